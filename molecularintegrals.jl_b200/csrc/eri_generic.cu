@@ -19,24 +19,41 @@
 //   (ab|cd) += c_a c_b c_c c_d 2 pi^(5/2) / (z e sqrt(z+e)) exp(-ab/z AB^2 - cd/e CD^2)
 //              sum_r W_r Ix Iy Iz.
 //
-// The block walks its outputs in tiles of kGenTile (a register accumulator per thread and output
-// of the tile) and, per tile, every primitive quartet.  Quartets with a g shell are rare in the
-// basis sets the engine serves; this kernel is written for generality, not speed.
+// A thread block takes one unit -- a tile of up to kGenTile outputs of one quartet -- at a time
+// from a queue.  The quartet's items (primitive quartet, root) are set up together, a thread each
+// (node, weight, recurrence coefficients), then go through shared memory in batches: a thread per
+// (item, axis) forms the columns of G in registers and transfers each to H; a thread per row of H
+// transfers it to I(ia, ib, ic, id); last every thread adds the batch's I_x I_y I_z to its outputs'
+// registers.  The transfers are paid once per 1-D entry ((gg|gg): 1875 per item) instead of once
+// per output (50,625), and the outputs of a quartet up to (gf|gd) are one tile, so most quartets
+// build their tables once.  Bound by the latency of a unit's phases (46 us for a (gg|gg) tile alone
+// on the device, half of it the FP64 divisions, exponentials and root series of the set-up).
+// Measured on B200, two centres with an s, p, d, f and g shell each (70 functions, 874 quartets
+// here): 0.185 ms, against 15.9 ms for a form that built G with one thread per axis and
+// transferred per output; kernels of 128 registers and two blocks per SM 0.185, three blocks of 80
+// registers (spilling) 0.34 against 0.31 ms with index tables instead of the register transfers.
 #include <cuda_runtime.h>
 
 #include "../../include/molints.h"
 #include "eri_common.cuh"
+#include "eri_generic.cuh"
 
 namespace molints {
 
 constexpr int kGenThreads = 256;
-constexpr int kGenAcc = 4;                        // outputs per thread and tile
-constexpr int kGenTile = kGenThreads * kGenAcc;   // outputs per tile
+constexpr int kGenAcc = 16;                       // outputs per thread and tile
+static_assert(kGenTile == kGenThreads * kGenAcc, "a tile is one register accumulator per thread and output");
 constexpr int kGenL = 4;                          // highest shell angular momentum
 constexpr int kGenE = 2 * kGenL;                  // la + lb
-constexpr int kGenNr = 2 * kGenL + 1;             // roots: (4 kGenL) / 2 + 1
 constexpr int kGenRysXmax = 100;
 constexpr int kGenNcheb = 16;
+constexpr int kGenItems = 96;                     // (primitive quartet, root) items set up at once
+// doubles of each of the two table regions (H and I): the 1-D tables of three (gg|gg) items
+// (3 * 5^4 doubles each), more items of smaller quartets.  Two blocks per SM.
+constexpr int kGenRegion = 5760;
+constexpr int kGenBatch = 64;                     // items whose tables are built at once, at most
+constexpr int kGenPar = 10;                       // per item: C00 x 3, D00 x 3, B00, B10, B01, weight
+constexpr int kGenPairs = 225;                    // component pairs of a (gg) shell pair
 
 // Cartesian components of l = 0..4 in the reference's shell_indices order, flat (35 entries):
 // x | y << 4 | z << 8, those of shell l starting at c_gen_comp_off[l].
@@ -44,19 +61,6 @@ __constant__ unsigned short c_gen_comp[35] = {0x0, 0x1, 0x10, 0x100, 0x2, 0x11, 
 // 1/sqrt((2I-1)!!(2J-1)!!(2K-1)!!) of each component
 __constant__ double c_gen_norm[35] = {0x1.0000000000000p+0, 0x1.0000000000000p+0, 0x1.0000000000000p+0, 0x1.0000000000000p+0, 0x1.279a74590331dp-1, 0x1.0000000000000p+0, 0x1.0000000000000p+0, 0x1.279a74590331dp-1, 0x1.0000000000000p+0, 0x1.279a74590331dp-1, 0x1.08654a2d4f6dap-2, 0x1.279a74590331dp-1, 0x1.279a74590331dp-1, 0x1.279a74590331dp-1, 0x1.279a74590331dp-1, 0x1.0000000000000p+0, 0x1.08654a2d4f6dap-2, 0x1.279a74590331dp-1, 0x1.279a74590331dp-1, 0x1.08654a2d4f6dap-2, 0x1.8fba8a1bf6f97p-4, 0x1.08654a2d4f6dap-2, 0x1.08654a2d4f6dap-2, 0x1.5555555555555p-2, 0x1.279a74590331dp-1, 0x1.5555555555555p-2, 0x1.08654a2d4f6dap-2, 0x1.279a74590331dp-1, 0x1.279a74590331dp-1, 0x1.08654a2d4f6dap-2, 0x1.8fba8a1bf6f97p-4, 0x1.08654a2d4f6dap-2, 0x1.5555555555555p-2, 0x1.08654a2d4f6dap-2, 0x1.8fba8a1bf6f97p-4};
 __constant__ int c_gen_comp_off[kGenL + 2] = {0, 1, 4, 10, 20, 35};
-
-// The per-quartet work of the generic kernel.
-struct GenQuartets {
-    const int4 *quartet;          // global shells (I, J, K, L), reference order
-    const int *mol;               // molecule of each quartet
-    long long n;
-    const double *xyz;            // shells: centre
-    const int *L, *nprim, *poff, *fn_off;  // angular momentum, primitives, first function in molecule
-    const double *expn, *ncoef;   // primitive exponents, normalised coefficients
-    const long long *mol_out;     // packed offset of each molecule
-    double *out;
-    RysTab rys;
-};
 
 // Node u_r and weight W_r of the n-point Rys rule at X (the tables of rys_root<NR> in
 // rys_common.cuh, n a run-time value).
@@ -86,163 +90,218 @@ __device__ void gen_root(const RysTab &R, int n, double X, int r, double &u, dou
     }
 }
 
-__device__ __forceinline__ double gen_binom(int n, int k) {
-    double r = 1.0;
-    for (int i = 1; i <= k; ++i) r = r * (double)(n - k + i) / (double)i;
-    return r;
+// Transfer of one 1-D column v[0 .. l0 + l1] (AB = the shells' distance on the axis): out[i *
+// (l1 + 1) * stride + j * stride] for i <= l0, j <= l1, by v_(j+1)[i] = v_j[i + 1] + AB v_j[i].
+__device__ __forceinline__ void gen_transfer(double *v, int l0, int l1, double AB, double *__restrict__ out,
+                                             int stride) {
+    const int si = (l1 + 1) * stride;
+    for (int j = 0;; ++j) {
+#pragma unroll
+        for (int i = 0; i <= kGenL; ++i)
+            if (i <= l0) out[i * si + j * stride] = v[i];
+        if (j == l1) break;
+#pragma unroll
+        for (int i = 0; i < kGenE; ++i) v[i] = fma(AB, v[i], v[i + 1]);  // beyond l0 + l1 - j: unused
+    }
 }
 
-__global__ void __launch_bounds__(kGenThreads) eri_generic_kernel(const GenQuartets Gq) {
-    // one root at a time, per axis: G[(E+1)(F+1)] then H[(la+1)(lb+1)(F+1)]
-    __shared__ double sG[3][(kGenE + 1) * (kGenE + 1)];
-    __shared__ double sH[3][(kGenL + 1) * (kGenL + 1) * (kGenE + 1)];
-    __shared__ double sRoot[kGenNr], sW[kGenNr];
-    __shared__ double sPar[16];
+__global__ void __launch_bounds__(kGenThreads, 2) eri_generic_kernel(const GenQuartets Gq) {
+    extern __shared__ __align__(16) double gen_smem[];
+    double *const tabI = gen_smem, *const tabH = gen_smem + kGenRegion;
+    __shared__ double sPar[kGenItems][kGenPar];
+    // per component pair of the bra and of the ket: offsets in the x, y and z tables (10 bits each,
+    // the bra's and the ket's add up: IS <= 625), function-pair index (-1: a duplicate), norm
+    __shared__ unsigned sOff[2][kGenPairs];
+    __shared__ int sFn[2][kGenPairs];
+    __shared__ double sNorm[2][kGenPairs];
+    __shared__ int s_unit;
     const int tid = threadIdx.x;
-    for (long long qi = blockIdx.x; qi < Gq.n; qi += gridDim.x) {
+    for (;;) {
+        __syncthreads();  // the previous unit's readers are done
+        if (tid == 0) s_unit = atomicAdd(Gq.counter, 1);
+        __syncthreads();
+        if (s_unit >= Gq.n) return;
+        // the list is in reference order, where the shells of high l tend to come last in each
+        // atom: taken from its end, the heavy quartets start first
+        const long long qi = Gq.n - 1 - s_unit;
         const int4 q = __ldg(&Gq.quartet[qi]);
+        const int2 mt = __ldg(&Gq.mol_tile[qi]);
         const int sh[4] = {q.x, q.y, q.z, q.w};
-        int l[4], np[4], po[4], fo[4];
-        double X0[4][3];
+        int l[4], np[4], po[4];
+#pragma unroll
         for (int t = 0; t < 4; ++t) {
             l[t] = __ldg(&Gq.L[sh[t]]);
             np[t] = __ldg(&Gq.nprim[sh[t]]);
             po[t] = __ldg(&Gq.poff[sh[t]]);
-            fo[t] = __ldg(&Gq.fn_off[sh[t]]);
-            for (int k = 0; k < 3; ++k) X0[t][k] = __ldg(&Gq.xyz[3 * sh[t] + k]);
         }
         const int nc[4] = {(l[0] + 1) * (l[0] + 2) / 2, (l[1] + 1) * (l[1] + 2) / 2,
                            (l[2] + 1) * (l[2] + 2) / 2, (l[3] + 1) * (l[3] + 2) / 2};
         const int E = l[0] + l[1], F = l[2] + l[3], nr = (E + F) / 2 + 1;
-        const int nout = nc[0] * nc[1] * nc[2] * nc[3];
-        const int F1 = F + 1, HS = (l[0] + 1) * (l[1] + 1) * F1;
-        double AB[3], CD[3], ab2 = 0.0, cd2 = 0.0;
-        for (int k = 0; k < 3; ++k) {
-            AB[k] = X0[0][k] - X0[1][k];
-            CD[k] = X0[2][k] - X0[3][k];
-            ab2 += AB[k] * AB[k];
-            cd2 += CD[k] * CD[k];
-        }
-        const bool same_ab = q.x == q.y, same_cd = q.z == q.w, same_pq = q.x == q.z && q.y == q.w;
-        const long long obase = __ldg(&Gq.mol_out[__ldg(&Gq.mol[qi])]);
-        for (int t0 = 0; t0 < nout; t0 += kGenTile) {
-            double acc[kGenAcc];
-            for (int j = 0; j < kGenAcc; ++j) acc[j] = 0.0;
-            for (int pa = 0; pa < np[0]; ++pa)
-                for (int pb = 0; pb < np[1]; ++pb)
-                    for (int pc = 0; pc < np[2]; ++pc)
-                        for (int pd = 0; pd < np[3]; ++pd) {
-                            __syncthreads();  // the previous primitive quartet's readers are done
-                            if (tid == 0) {
-                                const double a = __ldg(&Gq.expn[po[0] + pa]), b = __ldg(&Gq.expn[po[1] + pb]);
-                                const double c = __ldg(&Gq.expn[po[2] + pc]), d = __ldg(&Gq.expn[po[3] + pd]);
-                                const double z = a + b, e = c + d, ze = z + e;
-                                double P[3], Q[3], pq2 = 0.0;
-                                for (int k = 0; k < 3; ++k) {
-                                    P[k] = (a * X0[0][k] + b * X0[1][k]) / z;
-                                    Q[k] = (c * X0[2][k] + d * X0[3][k]) / e;
-                                    pq2 += (P[k] - Q[k]) * (P[k] - Q[k]);
-                                }
-                                const double coef = __ldg(&Gq.ncoef[po[0] + pa]) * __ldg(&Gq.ncoef[po[1] + pb]) *
-                                                    __ldg(&Gq.ncoef[po[2] + pc]) * __ldg(&Gq.ncoef[po[3] + pd]);
-                                sPar[0] = 2.0 * 17.493418327624862 /* pi^2.5 */ / (z * e * sqrt(ze)) *
-                                          exp(-a * b / z * ab2 - c * d / e * cd2) * coef;
-                                sPar[1] = z * e / ze * pq2;  // X
-                                sPar[2] = z;
-                                sPar[3] = e;
-                                for (int k = 0; k < 3; ++k) {
-                                    sPar[4 + k] = P[k] - X0[0][k];      // PA
-                                    sPar[7 + k] = Q[k] - X0[2][k];      // QC
-                                    sPar[10 + k] = Q[k] - P[k];         // Q - P
-                                }
-                            }
-                            __syncthreads();
-                            if (tid < nr) gen_root(Gq.rys, nr, sPar[1], tid, sRoot[tid], sW[tid]);
-                            __syncthreads();
-                            const double pref = sPar[0];
-                            for (int r = 0; r < nr; ++r) {
-                                __syncthreads();  // the previous root's readers are done
-                                if (tid < 3) {
-                                    // G table of root r on axis tid, serially
-                                    const int k = tid;
-                                    const double u = sRoot[r], z = sPar[2], e = sPar[3], ze = z + e;
-                                    const double B00 = 0.5 * u / ze, B10 = (1.0 - e * u / ze) / (2.0 * z),
-                                                 B01 = (1.0 - z * u / ze) / (2.0 * e);
-                                    const double C00 = sPar[4 + k] + e * sPar[10 + k] * u / ze;
-                                    const double D00 = sPar[7 + k] - z * sPar[10 + k] * u / ze;
-                                    double *g = sG[k];
-                                    g[0] = 1.0;
-                                    for (int i = 1; i <= E; ++i)
-                                        g[i * F1] = C00 * g[(i - 1) * F1] + (i > 1 ? (i - 1) * B10 * g[(i - 2) * F1] : 0.0);
-                                    for (int kk = 1; kk <= F; ++kk)
-                                        for (int i = 0; i <= E; ++i) {
-                                            double v = D00 * g[i * F1 + kk - 1];
-                                            if (kk > 1) v += (kk - 1) * B01 * g[i * F1 + kk - 2];
-                                            if (i > 0) v += i * B00 * g[(i - 1) * F1 + kk - 1];
-                                            g[i * F1 + kk] = v;
-                                        }
-                                }
-                                __syncthreads();
-                                // bra transfer H(ia, ib, k) on every axis
-                                for (int x = tid; x < 3 * HS; x += kGenThreads) {
-                                    const int k = x / HS, h = x - k * HS;
-                                    const int ia = h / ((l[1] + 1) * F1), rem = h - ia * (l[1] + 1) * F1;
-                                    const int ib = rem / F1, kk = rem - ib * F1;
-                                    double v = 0.0, p = 1.0;
-                                    for (int s = ib; s >= 0; --s) {  // C(ib, s) AB^(ib - s) G(ia + s, kk)
-                                        v += gen_binom(ib, s) * p * sG[k][(ia + s) * F1 + kk];
-                                        p *= AB[k];
-                                    }
-                                    sH[k][h] = v;
-                                }
-                                __syncthreads();
-                                const double wr = pref * sW[r];
-                                for (int j = 0; j < kGenAcc; ++j) {
-                                    const int o = t0 + j * kGenThreads + tid;
-                                    if (o >= nout) break;
-                                    const int id = o % nc[3], ic = (o / nc[3]) % nc[2],
-                                              ib = (o / (nc[3] * nc[2])) % nc[1], ia = o / (nc[3] * nc[2] * nc[1]);
-                                    const unsigned ca = c_gen_comp[c_gen_comp_off[l[0]] + ia],
-                                                   cb = c_gen_comp[c_gen_comp_off[l[1]] + ib],
-                                                   cc = c_gen_comp[c_gen_comp_off[l[2]] + ic],
-                                                   cd = c_gen_comp[c_gen_comp_off[l[3]] + id];
-                                    double prod = wr;
-                                    for (int k = 0; k < 3; ++k) {
-                                        const int ax = (ca >> (4 * k)) & 15, bx = (cb >> (4 * k)) & 15,
-                                                  cx = (cc >> (4 * k)) & 15, dx = (cd >> (4 * k)) & 15;
-                                        const double *h = sH[k] + (ax * (l[1] + 1) + bx) * F1;
-                                        double v = 0.0, p = 1.0;
-                                        for (int t = dx; t >= 0; --t) {  // C(dx, t) CD^(dx - t) H(.., cx + t)
-                                            v += gen_binom(dx, t) * p * h[cx + t];
-                                            p *= CD[k];
-                                        }
-                                        prod *= v;
-                                    }
-                                    acc[j] += prod;
-                                }
-                            }
-                        }
-            // the tile's unique integrals, normalised, at their iindex positions
-            for (int j = 0; j < kGenAcc; ++j) {
-                const int o = t0 + j * kGenThreads + tid;
-                if (o >= nout) break;
-                const int id = o % nc[3], ic = (o / nc[3]) % nc[2], ib = (o / (nc[3] * nc[2])) % nc[1],
-                          ia = o / (nc[3] * nc[2] * nc[1]);
-                const int i = fo[0] + ia, jj = fo[1] + ib, k = fo[2] + ic, ll = fo[3] + id;
-                if ((same_ab && i < jj) || (same_cd && k < ll)) continue;
-                const long long ij = pair_index(i, jj), kl = pair_index(k, ll);
-                if (same_pq && ij < kl) continue;
-                const double nrm = c_gen_norm[c_gen_comp_off[l[0]] + ia] * c_gen_norm[c_gen_comp_off[l[1]] + ib] *
-                                   c_gen_norm[c_gen_comp_off[l[2]] + ic] * c_gen_norm[c_gen_comp_off[l[3]] + id];
-                Gq.out[obase + packed_index(ij, kl)] = acc[j] * nrm;
+        const int nab = nc[0] * nc[1], ncd = nc[2] * nc[3], nout = nab * ncd;
+        const int F1 = F + 1, AB2 = (l[0] + 1) * (l[1] + 1), CD2 = (l[2] + 1) * (l[3] + 1);
+        const int HS = AB2 * F1, IS = AB2 * CD2;
+        const int t0 = mt.y * kGenTile, tn = min(kGenTile, nout - t0);
+        const int nj = (tn + kGenThreads - 1) / kGenThreads;  // outputs of a thread
+        // the unit's component-pair tables
+        for (int w = tid; w < 2 * kGenPairs; w += kGenThreads) {
+            const int side = w >= kGenPairs, x = w - side * kGenPairs;
+            const int l0 = l[2 * side], l1 = l[2 * side + 1], n1 = nc[2 * side + 1];
+            if (x < nc[2 * side] * n1) {
+                const int i0 = x / n1, i1 = x - i0 * n1;
+                const int c0 = c_gen_comp_off[l0] + i0, c1 = c_gen_comp_off[l1] + i1;
+                const unsigned m0 = c_gen_comp[c0], m1 = c_gen_comp[c1];
+                unsigned off = 0;
+#pragma unroll
+                for (int k = 0; k < 3; ++k)
+                    off |= ((((m0 >> (4 * k)) & 15) * (l1 + 1) + ((m1 >> (4 * k)) & 15)) * (side ? 1 : CD2)) << (10 * k);
+                const int f0 = __ldg(&Gq.fn_off[sh[2 * side]]) + i0, f1 = __ldg(&Gq.fn_off[sh[2 * side + 1]]) + i1;
+                sOff[side][x] = off;
+                // same-shell pairs: the larger component first; nbf <= 46000, so the index fits
+                sFn[side][x] = (sh[2 * side] == sh[2 * side + 1] && f0 < f1) ? -1 : (int)pair_index(f0, f1);
+                sNorm[side][x] = c_gen_norm[c0] * c_gen_norm[c1];
             }
+        }
+        __syncthreads();
+        // this thread's outputs: component pairs (bra | ket << 8) and table offsets
+        unsigned off[kGenAcc];
+        double acc[kGenAcc];
+#pragma unroll
+        for (int j = 0; j < kGenAcc; ++j) {
+            acc[j] = 0.0;
+            const int o = j * kGenThreads + tid;
+            const int ab = o < tn ? (t0 + o) / ncd : 0, cd = o < tn ? t0 + o - ab * ncd : 0;
+            off[j] = sOff[0][ab] + sOff[1][cd];
+        }
+        const int nitem = np[0] * np[1] * np[2] * np[3] * nr;
+        const int batch = min(kGenBatch, kGenRegion / (3 * IS));  // HS <= IS
+        for (int g0 = 0; g0 < nitem; g0 += kGenItems) {
+            const int ng = min(kGenItems, nitem - g0);
+            if (tid < ng) {
+                // item: primitive quartet (the last shell's primitive fastest) and root.  The previous
+                // items' readers (the H phase) are done: a barrier follows every H phase.
+                int pq = (g0 + tid) / nr;
+                const int r = g0 + tid - pq * nr;
+                const int pd = pq % np[3]; pq /= np[3];
+                const int pc = pq % np[2]; pq /= np[2];
+                const int pb = pq % np[1], pa = pq / np[1];
+                const double a = __ldg(&Gq.expn[po[0] + pa]), b = __ldg(&Gq.expn[po[1] + pb]);
+                const double c = __ldg(&Gq.expn[po[2] + pc]), d = __ldg(&Gq.expn[po[3] + pd]);
+                const double z = a + b, e = c + d, ze = z + e;
+                double ab2 = 0.0, cd2 = 0.0, pq2 = 0.0, PA[3], QC[3], QP[3];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const double A = __ldg(&Gq.xyz[3 * sh[0] + k]), B = __ldg(&Gq.xyz[3 * sh[1] + k]);
+                    const double C = __ldg(&Gq.xyz[3 * sh[2] + k]), D = __ldg(&Gq.xyz[3 * sh[3] + k]);
+                    const double P = (a * A + b * B) / z, Q = (c * C + d * D) / e;
+                    ab2 += (A - B) * (A - B);
+                    cd2 += (C - D) * (C - D);
+                    PA[k] = P - A;
+                    QC[k] = Q - C;
+                    QP[k] = Q - P;
+                    pq2 += (P - Q) * (P - Q);
+                }
+                const double coef = __ldg(&Gq.ncoef[po[0] + pa]) * __ldg(&Gq.ncoef[po[1] + pb]) *
+                                    __ldg(&Gq.ncoef[po[2] + pc]) * __ldg(&Gq.ncoef[po[3] + pd]);
+                const double pref = 2.0 * 17.493418327624862 /* pi^2.5 */ / (z * e * sqrt(ze)) *
+                                    exp(-a * b / z * ab2 - c * d / e * cd2) * coef;
+                double u, w;
+                gen_root(Gq.rys, nr, z * e / ze * pq2, r, u, w);
+                const double uze = u / ze;
+                double *par = sPar[tid];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    par[k] = PA[k] + e * QP[k] * uze;
+                    par[3 + k] = QC[k] - z * QP[k] * uze;
+                }
+                par[6] = 0.5 * uze;
+                par[7] = (1.0 - e * uze) / (2.0 * z);
+                par[8] = (1.0 - z * uze) / (2.0 * e);
+                par[9] = pref * w;
+            }
+            for (int b0 = 0; b0 < ng; b0 += batch) {
+                const int nb = min(batch, ng - b0);
+                __syncthreads();  // the items are set up; the previous batch's readers of H are done
+                // G of every (item, axis) column by column in registers (the x tables carry the
+                // weight), each column transferred to H(ia, ib, k) as it is formed
+                for (int ga = tid; ga < 3 * nb; ga += kGenThreads) {
+                    const int it = ga / 3, ax = ga - 3 * it;
+                    const double *par = sPar[b0 + it];
+                    const double C00 = par[ax], D00 = par[3 + ax], B00 = par[6], B10 = par[7], B01 = par[8];
+                    const double AB = __ldg(&Gq.xyz[3 * sh[0] + ax]) - __ldg(&Gq.xyz[3 * sh[1] + ax]);
+                    double *__restrict__ h = tabH + ga * HS;
+                    double cur[kGenE + 1], prev[kGenE + 1];
+                    cur[0] = ax == 0 ? par[9] : 1.0;
+                    cur[1] = C00 * cur[0];
+                    prev[0] = prev[1] = 0.0;
+#pragma unroll
+                    for (int i = 1; i < kGenE; ++i) {
+                        cur[i + 1] = i < E ? C00 * cur[i] + (double)i * B10 * cur[i - 1] : 0.0;
+                        prev[i + 1] = 0.0;
+                    }
+                    for (int k = 0;; ++k) {
+                        double v[kGenE + 1];
+#pragma unroll
+                        for (int i = 0; i <= kGenE; ++i) v[i] = cur[i];
+                        gen_transfer(v, l[0], l[1], AB, h + k, F1);
+                        if (k == F) break;
+#pragma unroll
+                        for (int i = 0; i <= kGenE; ++i) {
+                            v[i] = D00 * cur[i] + (double)k * B01 * prev[i];
+                            if (i > 0) v[i] += (double)i * B00 * cur[i - 1];
+                        }
+#pragma unroll
+                        for (int i = 0; i <= kGenE; ++i) {
+                            prev[i] = cur[i];
+                            cur[i] = v[i];
+                        }
+                    }
+                }
+                __syncthreads();
+                // ket transfer: I(ia, ib, ic, id) of every (item, axis, ia, ib)
+                for (int w = tid; w < 3 * nb * AB2; w += kGenThreads) {
+                    const int ax = (w / AB2) % 3;
+                    const double CD = __ldg(&Gq.xyz[3 * sh[2] + ax]) - __ldg(&Gq.xyz[3 * sh[3] + ax]);
+                    const double *__restrict__ h = tabH + w * F1;
+                    double v[kGenE + 1];
+#pragma unroll
+                    for (int k = 0; k <= kGenE; ++k) v[k] = k <= F ? h[k] : 0.0;
+                    gen_transfer(v, l[2], l[3], CD, tabI + w * CD2, 1);
+                }
+                __syncthreads();
+                for (int it = 0; it < nb; ++it) {
+                    const double *__restrict__ X = tabI + it * 3 * IS, *__restrict__ Y = X + IS, *__restrict__ Z = Y + IS;
+#pragma unroll
+                    for (int j = 0; j < kGenAcc; ++j) {
+                        if (j >= nj) break;
+                        const unsigned o = off[j];
+                        acc[j] = fma(X[o & 1023u] * Y[(o >> 10) & 1023u], Z[o >> 20], acc[j]);
+                    }
+                }
+            }
+        }
+        // the tile's unique integrals, normalised, at their iindex positions
+        const bool same_pq = q.x == q.z && q.y == q.w;
+        double *__restrict__ out = Gq.out + __ldg(&Gq.mol_out[mt.x]);
+#pragma unroll
+        for (int j = 0; j < kGenAcc; ++j) {
+            const int o = j * kGenThreads + tid;
+            if (o >= tn) break;
+            const int ab = (t0 + o) / ncd, cd = t0 + o - ab * ncd;
+            const int ij = sFn[0][ab], kl = sFn[1][cd];
+            if (ij < 0 || kl < 0 || (same_pq && ij < kl)) continue;
+            out[packed_index(ij, kl)] = acc[j] * (sNorm[0][ab] * sNorm[1][cd]);
         }
     }
 }
 
-void launch_eri_generic(const GenQuartets &G, int grid, cudaStream_t s) {
-    if (G.n <= 0 || grid <= 0) return;
-    eri_generic_kernel<<<grid, kGenThreads, 0, s>>>(G);
+constexpr int kGenSmem = 2 * kGenRegion * (int)sizeof(double);
+
+void launch_eri_generic(const GenQuartets &G, int num_sms, cudaStream_t s) {
+    if (G.n <= 0 || num_sms <= 0) return;
+    // (above 48 KB: allowed per function and device; plain state of the function, no queue work)
+    cudaFuncSetAttribute(eri_generic_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGenSmem);
+    const long long grid = G.n < 2LL * num_sms ? G.n : 2LL * num_sms;  // two resident blocks per SM
+    eri_generic_kernel<<<(int)grid, kGenThreads, kGenSmem, s>>>(G);
 }
 
 }  // namespace molints

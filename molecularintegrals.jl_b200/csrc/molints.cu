@@ -24,6 +24,7 @@
 #include "eri_common.cuh"
 #include "class_table.h"
 #include "eri_dispatch.h"
+#include "eri_generic.cuh"
 #include "plan_build.cuh"
 
 using namespace molints;
@@ -138,9 +139,10 @@ struct molints_plan {
     int n_launches = 0;
     int n_fp32_launches = 0;           // class-pair launches of the last execute that ran FP32
     // shell quartets with a g shell (l = 4): computed by the generic kernel (eri_generic.cu)
-    int64_t n_gq = 0;
-    int4 *gq = nullptr;                // global shells (I, J, K, L), reference order
-    int *gq_mol = nullptr;
+    int64_t n_gq = 0;                  // quartets
+    int64_t n_gunits = 0;              // units of at most kGenTile outputs
+    int4 *gq = nullptr;                // per unit: global shells (I, J, K, L), reference order
+    int2 *gq_mol = nullptr;            // per unit: molecule, tile of the quartet
     int *sh_L = nullptr, *sh_K = nullptr, *sh_fn = nullptr;  // shells' L and primitive count (all
                                                              // plans), first function (g plans)
     double plan_ms[4] = {0, 0, 0, 0};  // plan creation phases (molints_stats.plan_ms)
@@ -611,22 +613,6 @@ __global__ void boys_eval_kernel(BoysTab bt, int mmax, const double *__restrict_
     for (int m = 0; m < mmax; ++m) out[i * mmax + m] = F[m];
 }
 
-}  // namespace molints
-
-// ------------------------------------------------------------------ g shells (eri_generic.cu)
-namespace molints {
-struct GenQuartets {
-    const int4 *quartet;
-    const int *mol;
-    long long n;
-    const double *xyz;
-    const int *L, *nprim, *poff, *fn_off;
-    const double *expn, *ncoef;
-    const long long *mol_out;
-    double *out;
-    RysTab rys;
-};
-void launch_eri_generic(const GenQuartets &G, int grid, cudaStream_t s);
 }  // namespace molints
 
 // ------------------------------------------------------------------ helpers for noalloc.cu
@@ -1221,7 +1207,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     // holds one goes to the generic kernel, listed here in reference order (I >= J, K >= L,
     // pair IJ >= pair KL).
     std::vector<int4> gq_h;
-    std::vector<int> gq_mol_h;
+    std::vector<int2> gq_mol_h;
     for (int m = 0; m < nmol; ++m) {
         const int n = bases[m].nshell, s0 = shell_off[m];
         bool has_g = false;
@@ -1238,8 +1224,12 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
                     for (int k = 0; k <= i; ++k)
                         for (int l = 0; l <= (k == i ? j : k); ++l)
                             if (g_ij || L[s0 + k] > kLmax || L[s0 + l] > kLmax) {
-                                gq_h.push_back(make_int4(a, bb, s0 + k, s0 + l));
-                                gq_mol_h.push_back(m);
+                                const int nout = ncart(L[a]) * ncart(L[bb]) * ncart(L[s0 + k]) * ncart(L[s0 + l]);
+                                for (int t = 0; t * kGenTile < nout; ++t) {
+                                    gq_h.push_back(make_int4(a, bb, s0 + k, s0 + l));
+                                    gq_mol_h.push_back(make_int2(m, t));
+                                }
+                                ++p->n_gq;
                             }
                 }
                 if (g_ij) continue;
@@ -1247,7 +1237,11 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
                 pr.push_back({pair_class_of(L[a], L[bb]), m, K[a] * K[bb], a, bb, i * (i + 1) / 2 + j, i});
             }
     }
-    p->n_gq = (int64_t)gq_h.size();
+    p->n_gunits = (int64_t)gq_h.size();
+    if (p->n_gunits >= INT32_MAX) {
+        plan_free(p);
+        return fail(ctx, MOLINTS_ERR_INVALID, "plan_create: too many shell quartets with a g shell");
+    }
     if (p->n_gq > 0) p->two_phase = 0;  // the gather would overwrite the generic kernel's entries
     const bool sharded = nshards > 1;
     {
@@ -1567,7 +1561,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     rc = rc ? rc : dev_alloc(ctx, &p->pp_src, (size_t)nall, &p->bytes);
     rc = rc ? rc : dev_alloc(ctx, &p->pbk, (size_t)nall, &p->bytes);
     rc = rc ? rc : dev_alloc(ctx, &p->pp, (size_t)nall, &p->bytes);
-    rc = rc ? rc : dev_alloc(ctx, &p->counters, (size_t)nc2 + 1, &p->bytes);  // + the gather's
+    rc = rc ? rc : dev_alloc(ctx, &p->counters, (size_t)nc2 + 1, &p->bytes);  // + the gather's or the g kernel's
     rc = rc ? rc : dev_alloc(ctx, &p->mol_out, (size_t)std::max(nmol, 1), &p->bytes);
     if (tp) {
         rc = rc ? rc : dev_alloc(ctx, &p->g_fn, (size_t)std::max<int64_t>(nfn_all, 1), &p->bytes);
@@ -1765,12 +1759,12 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     if (p->n_gq > 0) {
         // the generic kernel's shell data and quartet list (pageable sources: each copy is
         // staged before the call returns)
-        rc = dev_alloc(ctx, &p->gq, (size_t)p->n_gq, &p->bytes);
-        if (!rc) rc = dev_alloc(ctx, &p->gq_mol, (size_t)p->n_gq, &p->bytes);
+        rc = dev_alloc(ctx, &p->gq, (size_t)p->n_gunits, &p->bytes);
+        if (!rc) rc = dev_alloc(ctx, &p->gq_mol, (size_t)p->n_gunits, &p->bytes);
         if (!rc) rc = dev_alloc(ctx, &p->sh_fn, (size_t)ns, &p->bytes);
         if (rc) { plan_free(p); return rc; }
         if ((e = cudaMemcpyAsync(p->gq, gq_h.data(), gq_h.size() * sizeof(int4), cudaMemcpyHostToDevice, s)) ||
-            (e = cudaMemcpyAsync(p->gq_mol, gq_mol_h.data(), gq_mol_h.size() * sizeof(int), cudaMemcpyHostToDevice, s)) ||
+            (e = cudaMemcpyAsync(p->gq_mol, gq_mol_h.data(), gq_mol_h.size() * sizeof(int2), cudaMemcpyHostToDevice, s)) ||
             (e = cudaMemcpyAsync(p->sh_fn, fn_off.data(), (size_t)ns * sizeof(int), cudaMemcpyHostToDevice, s)) ||
             (e = cudaStreamSynchronize(s))) {
             plan_free(p);
@@ -1839,13 +1833,26 @@ static int plan_enqueue(molints_plan *p, double *out_device, bool timing, JKOut 
             if (p->q_len[x][y] > 0) jobs.push_back({p->class_cost[x][y], x, y});
     std::stable_sort(jobs.begin(), jobs.end(), [](const Job &a, const Job &b) { return a.cost > b.cost; });
     // Profiling runs every launch on the caller's stream, so each event pair times one kernel.
-    const int nside = p->profiling ? 0 : std::min<int>(molints_ctx::kSide, (int)jobs.size());
+    const int ngen = p->n_gq > 0;
+    const int nside = p->profiling ? 0 : std::min<int>(molints_ctx::kSide, (int)jobs.size() + ngen);
     int fp32_launches = 0;
     if (nside > 0) MI_CUDA(ctx, cudaEventRecord(ctx->fork, s));
     for (int i = 0; i < nside; ++i) MI_CUDA(ctx, cudaStreamWaitEvent(ctx->side[i], ctx->fork, 0));
+    if (ngen) {
+        // shell quartets with a g shell (never two-phase plans; no J/K digestion): entries of their
+        // own, beside the class kernels on the first side stream
+        cudaStream_t st = nside ? ctx->side[0] : s;
+        GenQuartets G{p->gq, p->gq_mol, p->n_gunits, p->counters + kNumPairClasses * kNumPairClasses,
+                      p->sh_xyz, p->sh_L, p->sh_K, p->sh_poff, p->sh_fn, p->expn, p->ncoef, p->mol_out,
+                      out_device, ctx->rys};
+        if (int rc = mark(launches, "eri_generic", 0, st)) return rc;
+        launch_eri_generic(G, ctx->num_sms, st);
+        if (int rc = mark(launches, "eri_generic", 1, st)) return rc;
+        ++launches;
+    }
     for (size_t k = 0; k < jobs.size(); ++k) {
         const int x = jobs[k].x, y = jobs[k].y;
-        cudaStream_t st = nside ? ctx->side[k % nside] : s;
+        cudaStream_t st = nside ? ctx->side[(k + ngen) % nside] : s;
         const bool rys = p->method[x][y] == MOLINTS_METHOD_RYS;
         const int mixed = p->fp32[x][y];
         int &occ = ctx->occupancy[x][y][(rys ? 2 : 0) + mixed];
@@ -1880,15 +1887,6 @@ static int plan_enqueue(molints_plan *p, double *out_device, bool timing, JKOut 
     for (int i = 0; i < nside; ++i) {
         MI_CUDA(ctx, cudaEventRecord(ctx->join[i], ctx->side[i]));
         MI_CUDA(ctx, cudaStreamWaitEvent(s, ctx->join[i], 0));
-    }
-    if (p->n_gq > 0) {
-        // shell quartets with a g shell (never two-phase plans; no J/K digestion)
-        GenQuartets G{p->gq, p->gq_mol, p->n_gq, p->sh_xyz, p->sh_L, p->sh_K, p->sh_poff, p->sh_fn,
-                      p->expn, p->ncoef, p->mol_out, out_device, ctx->rys};
-        if (int rc = mark(launches, "eri_generic", 0, s)) return rc;
-        launch_eri_generic(G, (int)std::min<int64_t>(p->n_gq, (int64_t)ctx->num_sms * 8), s);
-        if (int rc = mark(launches, "eri_generic", 1, s)) return rc;
-        ++launches;
     }
     if (p->two_phase && !jk.J && p->npacked > 0) {
         // second phase: the packed vector in order from the scratch blocks
