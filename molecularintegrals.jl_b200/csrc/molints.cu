@@ -119,7 +119,9 @@ struct molints_plan {
     // class-major scratch, a gather pass writes the packed vector in order from it
     int two_phase = 0;
     int gather_blocks = 0;             // the context's schedule at creation: gather blocks per SM
+    int sharded = 0;
     int screen_trunc = 0;              // ket runs end at the last unscreened ket (quartet screening)
+    int64_t n_zero = 0;                // pairs without kept primitive pairs (in no chunk unless sharded)
     int64_t scratch_need = 0;          // doubles of the context's scratch an execute uses: per
                                        // (class pair, molecule) a region of quartet blocks
     long long *chunk_slot = nullptr;   // per chunk: scratch offset of its first quartet's block
@@ -338,7 +340,11 @@ __global__ void build_pairs_kernel(int npair, const int2 *__restrict__ pair_ab,
                                    const double *__restrict__ expn,
                                    const double *__restrict__ ncoef, double c0,
                                    const double *__restrict__ pb,
-                                   PrimPair *__restrict__ pp, double4 *__restrict__ geo) {
+                                   PrimPair *__restrict__ pp, double4 *__restrict__ geo,
+                                   double *__restrict__ clear, long long nclear) {
+    // a small direct output is cleared on the way (plan_enqueue)
+    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < nclear; k += (long long)gridDim.x * blockDim.x)
+        clear[k] = 0.0;
     // one warp per shell pair, its lanes over the pair's primitive pairs (up to 7 x 7)
     const int p = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
@@ -401,14 +407,15 @@ constexpr int kGatherThreads = 256;
 
 // Per function pair (i >= j) of every molecule of a two-phase plan, what the gather needs to
 // place its entries, built once per plan on the device: x = list position << 4 | pair class of
-// the shell pair holding (i, j), y = component of the function in that pair's A << 16 |
-// component in its B; colq (plans that screen quartets) the pair's Qabs.  Entry (m, ij) is at
+// the shell pair holding (i, j), or -1 if none of the pair's primitive pairs was kept (its quartets
+// are zero, and in no chunk), y = component of the function in that pair's A << 16 | component in
+// its B; colq (plans that screen quartets) the pair's Qabs.  Entry (m, ij) is at
 // col[mol[4m+3] + ij]; thread r takes entry r, of the molecule m with
 // mol[4m+3] <= r < mol[4(m+1)+3] (the molecules' entries follow one another).
 __global__ void gather_cols_kernel(int2 *__restrict__ col, double *__restrict__ colq,
-                                   const double2 *__restrict__ bnd, const int2 *__restrict__ fn,
-                                   const int *__restrict__ pairs, const long long *__restrict__ mol,
-                                   int nmol, long long nrows) {
+                                   const double2 *__restrict__ bnd, const int4 *__restrict__ info,
+                                   const int2 *__restrict__ fn, const int *__restrict__ pairs,
+                                   const long long *__restrict__ mol, int nmol, long long nrows) {
     const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= nrows) return;
     int m = 0, hi = nmol;  // last m with mol[4m+3] <= r
@@ -422,7 +429,8 @@ __global__ void gather_cols_kernel(int2 *__restrict__ col, double *__restrict__ 
     const int2 fi = __ldg(&fn[fb + i]), fj = __ldg(&fn[fb + j]);
     const int P = __ldg(&pairs[pb + (long long)fi.x * (fi.x + 1) / 2 + fj.x]);
     const int ca = (P & 1) ? fj.y : fi.y, cb = (P & 1) ? fi.y : fj.y;
-    col[__ldg(&mol[4 * m + 3]) + ij] = make_int2(((P >> 5) << 4) | ((P >> 1) & 15), (ca << 16) | cb);
+    const bool zero = __ldg(&info[P >> 5]).y == 0;
+    col[__ldg(&mol[4 * m + 3]) + ij] = make_int2(zero ? -1 : ((P >> 5) << 4) | ((P >> 1) & 15), (ca << 16) | cb);
     if (colq) colq[__ldg(&mol[4 * m + 3]) + ij] = __ldg(&bnd[P >> 5]).x;
 }
 
@@ -467,9 +475,11 @@ __device__ __forceinline__ void gather_pair_columns(
             kl[c] = kl0 + c * kGatherThreads;
             const bool on = kl[c] <= ijmax;
             const int2 qe = on ? __ldg(&col[cbase + kl[c]]) : make_int2(clsP, 0);
-            // a screened quartet (the class kernels' test, Qabs_P Qabs_Q < screen_cut) is 0;
-            // its block is not read (no chunk may have computed it)
-            zero[c] = on && screen_cut > 0.0 && qP * __ldg(&colq[cbase + kl[c]]) < screen_cut;
+            // a quartet of a pair without kept primitive pairs is 0, and so is a screened one (the
+            // class kernels' test, Qabs_P Qabs_Q < screen_cut); its block is not read (no chunk
+            // may have computed it)
+            const bool scr = on && screen_cut > 0.0 && qP * __ldg(&colq[cbase + kl[c]]) < screen_cut;
+            zero[c] = scr | (qe.x < 0);
             src[c] = scratch;
             rs[c] = 0;
             if (!zero[c]) {
@@ -537,7 +547,9 @@ __global__ void __launch_bounds__(kGatherThreads) gather_packed_kernel(
         // P's rows: ij, the row's first packed index tri(ij), and the row's component index in
         // P's A, B orientation
         const int2 pe = __ldg(&col[cbase + (long long)fi0 * (fi0 + 1) / 2 + fj0]);
-        const int posP = pe.x >> 4, clsP = pe.x & 15;
+        // a pair without kept primitive pairs: its rows are zeros (written below; class 0 stands in)
+        const bool zeroP = pe.x < 0;
+        const int posP = zeroP ? 0 : pe.x >> 4, clsP = zeroP ? 0 : pe.x & 15;
         const int nbP = c_pair_nb[clsP];
         const double qP = screen_cut > 0.0 ? __ldg(&bnd[posP]).x : 0.0;
         int R = 0;
@@ -562,10 +574,10 @@ __global__ void __launch_bounds__(kGatherThreads) gather_packed_kernel(
             }
         }
         __syncthreads();
-        if (screen_cut > 0.0 && qP * __ldg(&qmax[m]) < screen_cut) {
-            // every quartet of P is screened (Qabs_P times the molecule's largest Qabs is below
-            // the cutoff): its rows are zeros, written as contiguous runs with no descriptor or
-            // scratch loads
+        if (zeroP || (screen_cut > 0.0 && qP * __ldg(&qmax[m]) < screen_cut)) {
+            // P has no kept primitive pairs, or every quartet of P is screened (Qabs_P times the
+            // molecule's largest Qabs is below the cutoff): its rows are zeros, written as
+            // contiguous runs with no descriptor or scratch loads
             for (int r = 0; r < R; ++r) {
                 const long long t0 = s_tri[r], n = s_ij[r] + 1;
                 for (long long k = threadIdx.x; k < n; k += kGatherThreads) obase[t0 + k] = 0.0;
@@ -625,7 +637,7 @@ void launch_build_pairs(int npair, const int2 *pair_ab, const int4 *info, const 
     if (npair <= 0) return;
     build_pairs_kernel<<<build_pairs_blocks(npair), 128, 0, s>>>(npair, pair_ab, info, pp_src, xyz, poff,
                                                           expn, ncoef, std::sqrt(2.0) * std::pow(M_PI, 1.25),
-                                                          nullptr, pp, geo);
+                                                          nullptr, pp, geo, nullptr, 0);
 }
 
 // The scaled Boys tables of the kernels for M = 0..nM-1: row n of table M holds
@@ -1419,7 +1431,9 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     S.screen_sort = !sharded && opts.screen_cutoff > 0.0;
     S.screen_trunc = S.screen_sort;
     p->screen_trunc = S.screen_trunc;
+    p->sharded = sharded;
     S.screen_cut = opts.screen_cutoff;
+    S.zero_trunc = !sharded && !S.screen_sort;
 
     // ---- pinned upload buffer: the summary read back after the device build, the plan's
     // shells, the stage-1 block (laid out as in the device temporaries, one copy), the molecule
@@ -1445,12 +1459,13 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     const size_t t_ms = tv.take<int>(npair);
     const size_t t_cnt = tv.take<long long>((size_t)n_items + 1), t_cost = tv.take<double>(n_items);
     const size_t t_off = tv.take<long long>((size_t)n_items + 1);
-    const size_t t_sum = tv.take<long long>(kNumClassPairs + 1), t_ccost = tv.take<double>(kNumClassPairs);
+    const size_t t_sum = tv.take<long long>(kNumClassPairs + 2), t_ccost = tv.take<double>(kNumClassPairs);
     const size_t cub_bytes = std::max(plan_build_temp_bytes(npair), queue_count_temp_bytes(n_items));
     const size_t t_cub = tv.take<char>(cub_bytes);
     Carve sv;
-    // read back: class-pair chunk offsets, class-pair costs, kept primitive pairs, bad-shell flag
-    const size_t o_sum = sv.take<long long>(kNumClassPairs + 1), o_ccost = sv.take<double>(kNumClassPairs);
+    // read back: class-pair chunk offsets and the count of pairs without kept primitive pairs,
+    // class-pair costs, kept primitive pairs, bad-shell flag
+    const size_t o_sum = sv.take<long long>(kNumClassPairs + 2), o_ccost = sv.take<double>(kNumClassPairs);
     const size_t o_nkept = sv.take<long long>(1), o_bad = sv.take<int>(1);
     const size_t o_up = sv.take<char>(up_bytes);
     const size_t o_xyz = sv.take<double>(3 * (size_t)ns), o_expn = sv.take<double>(nprim);
@@ -1603,7 +1618,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
                 (e = h2d(p->g_units, o_gunits, (size_t)npe_all * sizeof(int4))))) ||
         (e = cudaMemsetAsync(p->counters + nc2, 0, sizeof(int), s)) ||
         (e = cudaMemsetAsync(tmp + t_qmax, 0, (size_t)std::max(nmol, 1) * sizeof(unsigned long long), s)) ||
-        (e = cudaMemsetAsync(tmp + t_sum, 0, (kNumClassPairs + 1) * sizeof(long long), s)) ||
+        (e = cudaMemsetAsync(tmp + t_sum, 0, (kNumClassPairs + 2) * sizeof(long long), s)) ||
         (e = cudaMemsetAsync(tmp + t_ccost, 0, kNumClassPairs * sizeof(double), s)) ||
         (e = cudaMemsetAsync(tmp + t_prefix, 0, sizeof(long long), s))) {
         release_temp(); plan_free(p);
@@ -1628,6 +1643,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     A.xyz = p->sh_xyz;
     A.sh_L = p->sh_L;
     A.qmax = reinterpret_cast<unsigned long long *>(tmp + t_qmax);
+    A.n_zero = reinterpret_cast<unsigned long long *>(tmp + t_sum) + kNumClassPairs + 1;
     A.npp1 = reinterpret_cast<int *>(tmp + t_npp1);
     A.bnd1 = reinterpret_cast<double2 *>(tmp + t_bnd1);
     A.key1 = reinterpret_cast<unsigned long long *>(tmp + t_key1);
@@ -1666,7 +1682,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
         }
         build_pairs_kernel<<<build_pairs_blocks(npair), 128, 0, s>>>(npair, A.ab1, A.info1, A.src1, p->sh_xyz,
                                                                      p->sh_poff, p->expn, p->ncoef, c0, nullptr,
-                                                                     p->pp, p->geo);
+                                                                     p->pp, p->geo, nullptr, 0);
         PairTab P1{A.info1, p->geo, p->pp, p->bnd};
         BoysTab Bt = boys_of(ctx, opts.boys);
         double2 *pbound = reinterpret_cast<double2 *>(tmp + t_pbound);
@@ -1682,7 +1698,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
         }
     }
     if ((e = cudaGetLastError()) ||
-        (e = cudaMemcpyAsync(stage + o_sum, tmp + t_sum, (kNumClassPairs + 1) * sizeof(long long),
+        (e = cudaMemcpyAsync(stage + o_sum, tmp + t_sum, (kNumClassPairs + 2) * sizeof(long long),
                              cudaMemcpyDeviceToHost, s)) ||
         (e = cudaMemcpyAsync(stage + o_ccost, tmp + t_ccost, kNumClassPairs * sizeof(double),
                              cudaMemcpyDeviceToHost, s)) ||
@@ -1700,6 +1716,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     const double *qcost = reinterpret_cast<const double *>(stage + o_ccost);
     p->nprim_pair_kept = *reinterpret_cast<const long long *>(stage + o_nkept);
     const long long nq = qsum[kNumClassPairs];
+    p->n_zero = qsum[kNumClassPairs + 1];
     if (nq > INT32_MAX) {
         release_temp(); plan_free(p);
         return fail(ctx, MOLINTS_ERR_INVALID, "plan_create: work queue too long");
@@ -1742,7 +1759,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     }
     if (tp && nrows_all > 0) {
         gather_cols_kernel<<<(unsigned)((nrows_all + 255) / 256), 256, 0, s>>>(p->g_col, p->g_colq, p->bnd,
-                                                                            p->g_fn, p->g_pair,
+                                                                            p->info, p->g_fn, p->g_pair,
                                                                             p->g_mol, nmol, nrows_all);
         e = cudaGetLastError();
         if (!e && p->g_qmax)  // the molecules' Qabs bounds (doubles as bits) outlive the build
@@ -1807,21 +1824,33 @@ static int plan_enqueue(molints_plan *p, double *out_device, bool timing, JKOut 
     };
     if (timing) MI_CUDA(ctx, cudaEventRecord(ctx->ev0, s));
     MI_CUDA(ctx, cudaMemsetAsync(p->counters, 0, sizeof(int) * (kNumPairClasses * kNumPairClasses + 1), s));
-    // direct plans that screen quartets: the screened quartets past each bra's last unscreened
-    // ket are in no chunk, so their zeros come from clearing the whole output first (a
-    // streaming write instead of scattered 8-byte stores).  Two-phase plans' gather writes them
-    // (measured on B200: clearing first and leaving them out of the gather cost more than the
-    // gather's zero stores, which are coalesced)
-    if (p->screen_trunc && !p->two_phase && !jk.J && p->npacked > 0)
+    // Direct plans: the quartets no chunk holds (those of pairs without kept primitive pairs, and
+    // with quartet screening those past each bra's last unscreened ket) get their zeros from
+    // clearing the whole output first, a streaming write instead of scattered 8-byte stores: up to
+    // 8 MB by the pair build itself (no launch), larger ones by a memset beside it.  Two-phase plans' gather writes
+    // them (measured on B200: clearing first and leaving them out of the gather cost more than the
+    // gather's zero stores, which are coalesced).
+    const bool clear = !p->two_phase && !jk.J && p->npacked > 0 && (p->screen_trunc || (p->n_zero > 0 && !p->sharded));
+    const bool clear_in_build = clear && p->npair > 0 && p->npacked < (1 << 20);
+    const bool clear_beside = clear && !clear_in_build && !p->profiling;
+    if (clear_beside) {
+        MI_CUDA(ctx, cudaEventRecord(ctx->fork, s));
+        MI_CUDA(ctx, cudaStreamWaitEvent(ctx->side[0], ctx->fork, 0));
+        MI_CUDA(ctx, cudaMemsetAsync(out_device, 0, (size_t)p->npacked * sizeof(double), ctx->side[0]));
+        MI_CUDA(ctx, cudaEventRecord(ctx->join[0], ctx->side[0]));
+    } else if (clear && !clear_in_build) {
         MI_CUDA(ctx, cudaMemsetAsync(out_device, 0, (size_t)p->npacked * sizeof(double), s));
+    }
     if (p->npair > 0) {
         if (int rc = mark(launches, "build_pairs", 0, s)) return rc;
         build_pairs_kernel<<<build_pairs_blocks(p->npair), 128, 0, s>>>(
             p->npair, p->pair_ab, p->info, p->pp_src, p->sh_xyz, p->sh_poff, p->expn, p->ncoef,
-            std::sqrt(2.0) * std::pow(M_PI, 1.25), p->pbk, p->pp, p->geo);
+            std::sqrt(2.0) * std::pow(M_PI, 1.25), p->pbk, p->pp, p->geo, clear_in_build ? out_device : nullptr,
+            clear_in_build ? (long long)p->npacked : 0);
         if (int rc = mark(launches, "build_pairs", 1, s)) return rc;
         ++launches;
     }
+    if (clear_beside) MI_CUDA(ctx, cudaStreamWaitEvent(s, ctx->join[0], 0));
     PairTab P{p->info, p->geo, p->pp, p->bnd};
     BoysTab B = boys_of(ctx, p->opts.boys);
     // Class-pair queues, largest estimated work first, spread over the side streams so that

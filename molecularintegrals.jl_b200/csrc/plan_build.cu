@@ -62,6 +62,7 @@ __global__ void pair_screen_kernel(PlanBuildArgs A) {
     double f = 1.0;
     for (int l = 0; l < A.sh_L[ab.y]; ++l) f *= dab1;
     A.npp1[k] = kept;
+    if (kept == 0) atomicAdd(A.n_zero, 1ull);
     A.bnd1[k] = make_double2(qa, wa * f);
     const unsigned long long within =
         A.screen_sort ? ((unsigned long long)(255 - qabs_bucket(qa)) << 12) | (unsigned long long)(0xFFF - min(kept, 0xFFF))
@@ -134,6 +135,10 @@ __device__ void walk_item(const QueueSetup &S, const QueueArgs &A, int ci, int p
     }
     if (S.screen_trunc && kend > kbeg) kend = unscreened_end(A.bnd, S.screen_cut, pb, kbeg, kend);
     const int nb = A.npp[pb];
+    if (S.zero_trunc) {
+        if (nb == 0) return;
+        kend = nonzero_end(A.npp, kbeg, kend);
+    }
     const double wp = S.w[ci] * nb, pcost = S.pcost[ci];
     // this bra's remaining kets may still need a split (in Qabs order the kept counts do not
     // descend along the run: every chunk is tested)

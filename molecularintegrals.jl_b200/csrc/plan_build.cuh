@@ -93,6 +93,15 @@ __host__ __device__ inline int unscreened_end(const double2 *bnd, double cut, in
     return e;
 }
 
+// The first pair of [kbeg, kend) without kept primitive pairs, the run's kept counts descending.
+__host__ __device__ inline int nonzero_end(const int *npp, int kbeg, int kend) {
+    while (kbeg < kend) {
+        const int mid = (kbeg + kend) >> 1;
+        if (npp[mid] > 0) kbeg = mid + 1; else kend = mid;
+    }
+    return kbeg;
+}
+
 // What the queue kernels need per class pair (x, y <= x), in the host's class-pair order
 // (x outer, y inner): a plain struct passed by value.
 struct QueueSetup {
@@ -115,6 +124,12 @@ struct QueueSetup {
     // (two-phase plans) or from clearing the output before the class kernels (direct plans).
     int screen_sort, screen_trunc;
     double screen_cut;
+    // A pair none of whose primitive pairs was kept (prim_cutoff) makes every quartet it is in
+    // zero.  Runs in kept-count order (neither sharded nor screen_sort) have such pairs last: no
+    // chunk holds one, and the zeros are written as those of screened quartets are.  In the
+    // 256-molecule batch they are 40-60 % of a molecule's pairs (tight uncontracted shells on
+    // other centres) and 78 % of the integrals.
+    int zero_trunc;
 };
 
 // Device arrays of one device plan build (all owned by the caller).
@@ -133,6 +148,7 @@ struct PlanBuildArgs {
     const double *xyz;             // shell centres
     const int *sh_L;
     unsigned long long *qmax;      // per molecule, zeroed: max over pairs of sum b_k (bits)
+    unsigned long long *n_zero;    // zeroed: pairs without kept primitive pairs
     // re-sort scratch
     int *npp1;                     // kept count per stage-1 pair
     double2 *bnd1;                 // (Qabs, R) per stage-1 pair
