@@ -82,6 +82,7 @@ struct JKOut {
 struct EriQueue {
     PairTab pairs;
     BoysTab boys;
+    RysTab rys;                   // lane-split Rys kernels
     JKOut jk;                     // jk.J != nullptr: digest into J and K instead of storing
     double *out;                  // packed outputs of all molecules (device)
     const long long *mol_out;     // offset of each molecule's packed vector in out

@@ -79,12 +79,10 @@ void launch_eri_ffss(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_ffss(int mixed);
 void launch_rys_ssss(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_ssss(int mixed);
-void launch_rys_bound_ssss(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, double *qout, int full, cudaStream_t s);
 void launch_rys_psss(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_psss(int mixed);
 void launch_rys_psps(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_psps(int mixed);
-void launch_rys_bound_psps(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, double *qout, int full, cudaStream_t s);
 void launch_rys_ppss(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_ppss(int mixed);
 void launch_rys_ppps(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
@@ -287,6 +285,21 @@ static const float kEriPrimCost[11][11] = {
     {32.5f, 81.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f},
     {53.5f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f},
 };
+// the same of the Rys kernel where its queue is lane-split like an HGP kernel's (gen_rys.is_lane):
+// a root's two series cost about what twelve VRR entries do; 0 where a group computes whole quartets
+static const float kRysPrimCost[11][11] = {
+    {4.25f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f},
+    {4.75f, 11.5f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f},
+    {11.5f, 20.5f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f},
+    {10.0f, 16.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f},
+    {15.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f},
+    {12.0f, 32.5f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f},
+    {33.25f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f},
+    {28.75f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f},
+    {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f},
+    {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f},
+    {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f},
+};
 // 1 where the class pair's kernel has an FP32 variant for MIXED quartets (HGP: at least
 // 40 VRR entries; Rys: gen_rys's MIXED_MIN_NBLK / MIXED_MAX_ACC rule), else 0
 static const unsigned char kEriHasFp32[11][11] = {
@@ -361,6 +374,6 @@ static const SchwarzLauncher kSchwarzLaunchers[11] = {
     launch_schwarz_ssss, launch_schwarz_psps, launch_schwarz_pppp, launch_schwarz_dsds, launch_schwarz_dpdp, launch_schwarz_fsfs, launch_schwarz_dddd, nullptr, nullptr, nullptr, nullptr
 };
 static const RysBoundLauncher kRysBoundLaunchers[11] = {
-    launch_rys_bound_ssss, launch_rys_bound_psps, launch_rys_bound_pppp, launch_rys_bound_dsds, launch_rys_bound_dpdp, launch_rys_bound_fsfs, launch_rys_bound_dddd, launch_rys_bound_fpfp, launch_rys_bound_dfdf, launch_rys_bound_fdfd, launch_rys_bound_ffff
+    nullptr, nullptr, launch_rys_bound_pppp, launch_rys_bound_dsds, launch_rys_bound_dpdp, launch_rys_bound_fsfs, launch_rys_bound_dddd, launch_rys_bound_fpfp, launch_rys_bound_dfdf, launch_rys_bound_fdfd, launch_rys_bound_ffff
 };
 }  // namespace molints

@@ -263,9 +263,41 @@ class HrrPlan:
 
 
 # ------------------------------------------------------------------ emit
-def emit_class_pair(X, Y):
+def rys_lane_lines(X, Y, hp):
+    """One root's 2-D tables in registers (the recurrences of gen_rys) and its products into acc:
+    the body of the root loop of a lane-split Rys kernel."""
+    e, f = X[0] + X[1], Y[0] + Y[1]
+    out = []
+    for x in XYZ:
+        out.append(f"const double C{x} = fma(-ez * PQ{x}, u, bra.pa{x}), D{x} = fma(zz * PQ{x}, u, ket.pa{x});")
+        out.append(f"(void)C{x}; (void)D{x};")
+    for x in XYZ:
+        for c in range(f + 1):
+            for a in range(e + 1):
+                n = f"{x}{a}_{c}"
+                if a == c == 0:
+                    out.append(f"const double {n} = {'pref * w' if x == 'x' else '1.0'};")
+                elif c == 0:
+                    s = f"C{x} * {x}{a - 1}_0" + (f" + {a - 1}.0 * b10 * {x}{a - 2}_0" if a > 1 else "")
+                    out.append(f"const double {n} = {s};")
+                else:
+                    s = f"D{x} * {x}{a}_{c - 1}"
+                    s += f" + {c - 1}.0 * b01 * {x}{a}_{c - 2}" if c > 1 else ""
+                    s += f" + {a}.0 * b00 * {x}{a - 1}_{c - 1}" if a else ""
+                    out.append(f"const double {n} = {s};")
+    for a in hp.acc_a:
+        for c in hp.acc_c:
+            m, n = AO[a], AO[c]
+            out.append(f"acc[{hp.acc_index[(a, c)]}] = fma(x{m[0]}_{n[0]} * y{m[1]}_{n[1]}, z{m[2]}_{n[2]}, "
+                       f"acc[{hp.acc_index[(a, c)]}]);")
+    return out
+
+
+def emit_class_pair(X, Y, rys=False):
+    """The lane-split class kernel of (X|Y): HGP, or (rys) the same kernel with the primitive
+    quartets by Rys quadrature (gen_rys: class pairs of small blocks)."""
     (la, lb), (lc, ld) = X, Y
-    tag = tag_of(X, Y)
+    tag = tag_of(X, Y) + ("_rys" if rys else "")
     e, f = la + lb, lc + ld
     M = e + f
     entries = vrr_entries(la, e, lc, f)
@@ -309,7 +341,7 @@ def emit_class_pair(X, Y):
                         for ic in range(nc) for id_ in range(nd))
     store_code = "\n".join(stores)
     schwarz = ""
-    if X == Y:
+    if X == Y and not rys:
         diag = []
         for ia in range(na):
             for ib in range(nb):
@@ -356,11 +388,12 @@ void launch_schwarz_{tag}(const PairTab &P, const BoysTab &B, int p0, int np, do
     schwarz_kernel_{tag}<<<(np + 127) / 128, 128, 0, s>>>(P, B, p0, np, pbound, qout, full);
 }}
 """
+    has32 = len(entries) >= MIXED_MIN_VRR and not rys
     if nout <= STAGE_MAX_OUT:
         sbytes = 4 * 32 * nout * 8
         mixed_attr = (f"        cudaFuncSetAttribute(eri_queue_{tag}<1, 0>, "
                       f"cudaFuncAttributeMaxDynamicSharedMemorySize, {sbytes});\n"
-                      if len(entries) >= MIXED_MIN_VRR else "")
+                      if has32 else "")
         stage_fn = (f"""
 // The dynamic shared memory of the two-phase staging ({sbytes} bytes), allowed once per device
 // (before any graph capture: the occupancy query of plan creation calls it first).
@@ -404,7 +437,7 @@ static void eri_prepare_{tag}() {{
 #pragma unroll
                 for (int x = 0; x < {nout}; ++x) dst[x] = res[x];
             }}"""
-    if len(entries) >= MIXED_MIN_VRR:
+    if has32:
         mixed_dispatch = ("    const bool jk = Q.jk.J != nullptr;\n"
                           "    if (mixed) {{ if (jk) eri_queue_{t}<1, 1><<<grid, 128, 0, s>>>(Q); "
                           "else eri_queue_{t}<1, 0><<<grid, 128, smem, s>>>(Q); }}\n"
@@ -418,13 +451,41 @@ static void eri_prepare_{tag}() {{
                           "    else eri_queue_{t}<0, 0><<<grid, 128, smem, s>>>(Q);").format(t=tag)
         occ_dispatch = ("    (void)mixed;\n"
                         "    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, eri_queue_{t}<0, 0>, 128, 0);").format(t=tag)
-    return f"""// Generated by gen_eri.py -- class ({'spdfg'[la]}{'spdfg'[lb]}|{'spdfg'[lc]}{'spdfg'[ld]}).  Do not edit.
-// VRR entries: {len(entries)}, contracted block: {nacc}, HRR lines: {len(hp.lines)}, outputs: {nout}.
-#include "../eri_common.cuh"
-
-namespace molints {{
-
-// The contracted [e0|f0] block of bra pair p and ket pair q into acc[{nacc}], summed over
+    if rys:
+        nr = M // 2 + 1
+        body = "\n".join(ind + "        " + ln for ln in rys_lane_lines(X, Y, hp))
+        vrr_fn = f"""// The contracted [e0|f0] block of bra pair p and ket pair q into acc[{nacc}] by the {nr}-point Rys
+// rule, summed over the bra primitive pairs i0, i0 + istep, ... < i1 and the ket primitive pairs
+// j0, j0 + jstep, ... < j1; loop order and splits as in the HGP kernel of the class.
+__device__ __forceinline__ void vrr_{tag}(const PairTab &P, const RysTab &R, int p, int q, int i0, int i1,
+                                          int istep, int j0, int j1, int jstep, double *__restrict__ acc) {{
+    const int4 ib_ = __ldg(&P.info[p]);
+    const int4 ik_ = __ldg(&P.info[q]);
+#pragma unroll
+    for (int x = 0; x < {nacc}; ++x) acc[x] = 0.0;
+    for (int j = j0; j < j1; j += jstep) {{
+        const PrimPair ket = load_pp(P.pp, ik_.x + j);
+        for (int i = i0; i < i1; i += istep) {{
+            const PrimPair bra = load_pp(P.pp, ib_.x + i);
+            const double r = rsqrt(bra.zeta + ket.zeta);
+            const double r2 = r * r;
+            const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
+            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double pref = bra.kab * ket.kab * r;
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+#pragma unroll 1
+            for (int k = 0; k < {nr}; ++k) {{
+                double u, w;
+                rys_root<{nr}>(R, T, k, u, w);
+                const double b10 = bra.oo2z * fma(-ez, u, 1.0), b01 = ket.oo2z * fma(-zz, u, 1.0), b00 = 0.5 * r2 * u;
+                (void)b10; (void)b01; (void)b00;
+{body}
+            }}
+        }}
+    }}
+}}"""
+    else:
+        vrr_fn = f"""// The contracted [e0|f0] block of bra pair p and ket pair q into acc[{nacc}], summed over
 // the bra primitive pairs i0, i0 + istep, ... < i1 and the ket primitive pairs j0, j0 + jstep,
 // ... < j1 of the two shell pairs.  VT is the VRR arithmetic type (double, or float for MIXED).
 // The ket loop is outside: a warp shares its bra pair, so the inner bra loads are broadcasts
@@ -463,7 +524,46 @@ __device__ __forceinline__ void vrr_{tag}(const PairTab &P, const BoysTab &B, in
 {acc_code}
         }}
     }}
-}}
+}}"""
+    quartet_fn = "" if rys else f"""// (ab|cd) over the bra primitive pairs [i0, i1) and ket primitive pairs [j0, j1) into
+// res[{nout}]; the contracted block also into acc_out when given (the bound kernels).
+template <typename VT>
+__device__ __forceinline__ void quartet_{tag}(const PairTab &P, const BoysTab &B, int p, int q,
+                                              int i0, int i1, int j0, int j1,
+                                              double *__restrict__ res,
+                                              double *__restrict__ acc_out = nullptr) {{
+    double acc[{nacc}];
+    vrr_{tag}<VT>(P, B, p, q, i0, i1, 1, j0, j1, 1, acc);
+    if (acc_out) {{
+#pragma unroll
+        for (int x = 0; x < {nacc}; ++x) acc_out[x] = acc[x];
+    }}
+    hrr_{tag}(P, p, q, acc, res);
+}}"""
+    if rys:
+        head = (f"// Generated by gen_rys.py -- Rys class ({tag[0]}{tag[1]}|{tag[2]}{tag[3]}).  Do not edit.\n"
+                f"// roots {M // 2 + 1}, contracted block: {nacc}, outputs: {nout}: a lane-split kernel, the lanes' primitive quartets by\n"
+                f"// Rys quadrature with the 2-D tables in registers.\n"
+                f'#include "../rys_common.cuh"')
+        vrr_call = f"vrr_{tag}(Q.pairs, Q.rys, p, q, is, nb, 1 << (lg - lgj), js, nk, 1 << lgj, acc);"
+        launch_head = f"""void launch_rys_{tag_of(X, Y)}(const EriQueue &Q0, const RysTab &R, int mixed, int grid, cudaStream_t s) {{
+    EriQueue Q = Q0;
+    Q.rys = R;"""
+        occ_head = f"int occupancy_rys_{tag_of(X, Y)}(int mixed) {{"
+    else:
+        head = (f"// Generated by gen_eri.py -- class ({'spdfg'[la]}{'spdfg'[lb]}|{'spdfg'[lc]}{'spdfg'[ld]}).  Do not edit.\n"
+                f"// VRR entries: {len(entries)}, contracted block: {nacc}, HRR lines: {len(hp.lines)}, outputs: {nout}.\n"
+                f'#include "../eri_common.cuh"')
+        vrr_call = (f"if (MIXED && bp.y * bq.y < Q.fp32_cut)\n"
+                    f"                vrr_{tag}<float>(Q.pairs, Q.boys, p, q, is, nb, 1 << (lg - lgj), js, nk, 1 << lgj, acc);\n"
+                    f"            else vrr_{tag}<double>(Q.pairs, Q.boys, p, q, is, nb, 1 << (lg - lgj), js, nk, 1 << lgj, acc);")
+        launch_head = f"void launch_eri_{tag}(const EriQueue &Q, int mixed, int grid, cudaStream_t s) {{"
+        occ_head = f"int occupancy_eri_{tag}(int mixed) {{"
+    return f"""{head}
+
+namespace molints {{
+
+{vrr_fn}
 
 // Bra and ket HRR of the contracted block (src/HGP.jl:92-114), then the component norms:
 // the normalised (ab|cd) of bra pair p and ket pair q into res[{nout}] (ma, mb, mc, md
@@ -479,21 +579,7 @@ __device__ __forceinline__ void hrr_{tag}(const PairTab &P, int p, int q, const 
 {out_code}
 }}
 
-// (ab|cd) over the bra primitive pairs [i0, i1) and ket primitive pairs [j0, j1) into
-// res[{nout}]; the contracted block also into acc_out when given (the bound kernels).
-template <typename VT>
-__device__ __forceinline__ void quartet_{tag}(const PairTab &P, const BoysTab &B, int p, int q,
-                                              int i0, int i1, int j0, int j1,
-                                              double *__restrict__ res,
-                                              double *__restrict__ acc_out = nullptr) {{
-    double acc[{nacc}];
-    vrr_{tag}<VT>(P, B, p, q, i0, i1, 1, j0, j1, 1, acc);
-    if (acc_out) {{
-#pragma unroll
-        for (int x = 0; x < {nacc}; ++x) acc_out[x] = acc[x];
-    }}
-    hrr_{tag}(P, p, q, acc, res);
-}}
+{quartet_fn}
 
 __device__ __forceinline__ void store_{tag}(double *__restrict__ out, const int4 ib_, const int4 ik_,
                                             bool same, const double *__restrict__ res) {{
@@ -554,9 +640,7 @@ __global__ void __launch_bounds__(128) eri_queue_{tag}(const EriQueue Q) {{
             for (int x = 0; x < {nacc}; ++x) acc[x] = 0.0;
         }} else {{
             const int nb = __ldg(&Q.pairs.info[p]).y, nk = __ldg(&Q.pairs.info[q]).y;
-            if (MIXED && bp.y * bq.y < Q.fp32_cut)
-                vrr_{tag}<float>(Q.pairs, Q.boys, p, q, is, nb, 1 << (lg - lgj), js, nk, 1 << lgj, acc);
-            else vrr_{tag}<double>(Q.pairs, Q.boys, p, q, is, nb, 1 << (lg - lgj), js, nk, 1 << lgj, acc);
+            {vrr_call}
         }}
         if (lg) {{
             for (int off = W; off < 32; off <<= 1) {{
@@ -582,14 +666,14 @@ __global__ void __launch_bounds__(128) eri_queue_{tag}(const EriQueue Q) {{
 }}
 
 {stage_fn}
-void launch_eri_{tag}(const EriQueue &Q, int mixed, int grid, cudaStream_t s) {{
+{launch_head}
     if (Q.nchunks <= 0 || grid <= 0) return;
 {stage_prep}
 {mixed_dispatch}
 }}
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
-int occupancy_eri_{tag}(int mixed) {{
+{occ_head}
 {occ_prep}
     int n = 0;
 {occ_dispatch}
@@ -618,7 +702,7 @@ def emit_dispatch(pairs):
         t = tag_of(X, Y)
         lines.append(f"void launch_rys_{t}(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);")
         lines.append(f"int occupancy_rys_{t}(int mixed);")
-        if X == Y:
+        if X == Y and not gen_rys.is_lane(X, Y):
             lines.append(f"void launch_rys_bound_{t}(const PairTab &P, const RysTab &R, int p0, int np, "
                          f"double2 *pbound, double *qout, int full, cudaStream_t s);")
     lines.append("typedef void (*EriLauncher)(const EriQueue &, int, int, cudaStream_t);")
@@ -661,6 +745,19 @@ def emit_dispatch(pairs):
                 row.append("0.0f")
         lines.append("    {" + ", ".join(row) + "},")
     lines.append("};")
+    lines.append("// the same of the Rys kernel where its queue is lane-split like an HGP kernel's (gen_rys.is_lane):")
+    lines.append("// a root's two series cost about what twelve VRR entries do; 0 where a group computes whole quartets")
+    lines.append(f"static const float kRysPrimCost[{n}][{n}] = {{")
+    for i, X in enumerate(cls):
+        row = []
+        for j, Y in enumerate(cls):
+            if j <= i and gen_rys.is_lane(X, Y):
+                nr = (sum(X) + sum(Y)) // 2 + 1
+                row.append(f"{1.0 + nr * (12 + gen_rys.class_tables(X, Y)['nblk']) / 4.0!r}f")
+            else:
+                row.append("0.0f")
+        lines.append("    {" + ", ".join(row) + "},")
+    lines.append("};")
     lines.append("// 1 where the class pair's kernel has an FP32 variant for MIXED quartets (HGP: at least")
     lines.append(f"// {MIXED_MIN_VRR} VRR entries; Rys: gen_rys's MIXED_MIN_NBLK / MIXED_MAX_ACC rule), else 0")
     for name, has in (("kEriHasFp32", lambda X, Y: (X, Y) in hgp and
@@ -682,7 +779,8 @@ def emit_dispatch(pairs):
                                    for X in cls))
     lines.append("};")
     lines.append(f"static const RysBoundLauncher kRysBoundLaunchers[{n}] = {{")
-    lines.append("    " + ", ".join(f"launch_rys_bound_{tag_of(X, X)}" for X in cls))
+    lines.append("    " + ", ".join("nullptr" if gen_rys.is_lane(X, X) else f"launch_rys_bound_{tag_of(X, X)}"
+                                   for X in cls))
     lines.append("};")
     lines.append("}  // namespace molints")
     return "\n".join(lines) + "\n"

@@ -19,15 +19,17 @@ src/Rys.jl:27-156), reorganised for the GPU as Rys VRR + HGP HRR:
     bra side first, then ket side;
   * component norms and the packed iindex store, as in the HGP kernels.
 
-A group of G threads (32, 64 or 128; a block of 128 threads holds 128/G groups) owns one
-contracted shell quartet at a time.  Stage 1 of a primitive batch: one thread per
-(primitive quartet, root) evaluates the root and builds the three 2-D tables into shared
-memory; stage 2: every thread accumulates its own entries of the [e0|f0] block in registers
-(small blocks: NSLOT threads per entry, each over every NSLOT-th quartet of the batch).
-After the primitive loop the block goes to shared memory for the two HRR passes.
+A group of G threads (32, 64 or 128; a block of 128 threads holds 128/G groups) takes W ket
+pairs of one bra pair at a time (W > 1 where the block has few columns).  Stage 1 of a primitive
+batch: one thread per (ket pair, primitive quartet, root) evaluates the root and builds the three
+2-D tables into shared memory; stage 2: one thread per (ket pair, block column) loads the column's
+table columns once per root and updates all row accumulators of the column in registers.  The bra
+HRR then runs in that thread's registers, the ket HRR one thread per bra component pair on a row
+in shared memory, both as unrolled recurrences (up to 351 steps, (ff|, without spills).
 
-The class-specific data (block entry -> table offsets, HRR term lists, norms) are emitted as
-device arrays; the kernel body is the template in rys_common.cuh.
+The class-specific code (column update, the two HRR sides) and data (column components, norms) are
+emitted per class; the kernel body is the template in rys_common.cuh.  class_tables also states
+the block's table offsets and the HRR in closed form, which the tests evaluate.
 """
 from __future__ import annotations
 
@@ -42,7 +44,6 @@ NMONO = 20           # monomials AB^(px,py,pz), px+py+pz <= 3
 # thread get an FP32 variant for MIXED quartets (stage-2 products summed in FP32 per batch).
 MIXED_MIN_NBLK = 32
 MIXED_MAX_ACC = 24
-COL_MIN_NC = 16
 COL_MAX_NA = 48
 
 
@@ -125,6 +126,28 @@ def hrr_terms(lx, ly, rows_index):
     return out
 
 
+class HrrSide:
+    """Unrolled horizontal recurrence of one side, (a b| = (a+1 b-1| + AB (a b-1| (src/HGP.jl:92-114):
+    from the side's (a 0| entries in[] to every (a b|, a in shell lx, b in shell ly."""
+
+    def __init__(self, lx, ly, index):
+        self.index, self.lines, self.done = index, [], {}
+        self.out = [self.term(a, b) for a in shell_components(lx) for b in shell_components(ly)]
+
+    def term(self, a, b):
+        if sum(b) == 0:
+            return f"in[{self.index[a]}]"
+        if (a, b) not in self.done:
+            i = max(range(3), key=lambda t: (b[t], -t))
+            bm = tuple(b[t] - (t == i) for t in range(3))
+            ap = tuple(a[t] + (t == i) for t in range(3))
+            hi, lo = self.term(ap, bm), self.term(a, bm)
+            name = f"h{len(self.lines)}"
+            self.lines.append(f"const double {name} = fma({'xyz'[i]}, {lo}, {hi});")
+            self.done[(a, b)] = name
+        return self.done[(a, b)]
+
+
 def class_tables(X, Y):
     """Everything the kernel of class pair (X|Y) needs, as Python data."""
     (la, lb), (lc, ld) = X, Y
@@ -147,41 +170,35 @@ def class_tables(X, Y):
     na, nc = len(rows), len(cols)
     nblk = na * nc
     nab, ncd = ncart(la) * ncart(lb), ncart(lc) * ncart(ld)
-    # column mode: one stage-2 thread per block column holds that column's three 2-D table
-    # columns and all NA row accumulators in registers (3(E+1) shared loads per root instead
-    # of 3 per entry); for blocks with at least COL_MIN_NC columns and at most COL_MAX_NA rows
-    col = nc >= COL_MIN_NC and na <= COL_MAX_NA
-    if col:
-        G = 32 * ((nc + 31) // 32)
-    elif nblk <= 128:
-        G = 32
-    elif nblk <= 1024:
-        G = 64
-    else:
-        G = 128
-    # primitive quartets per batch: one stage-1 thread per (quartet, root); the batch's 2-D
-    # tables may use the HRR buffers' room (at least 6144 doubles)
-    hrr_room = max(nblk + nab * nc, 6144)
-    npb = max(1, min(G // nr, hrr_room // (3 * nr * S)))
-    # stage-2 slots: a small block is accumulated by NSLOT threads per entry, each taking every
-    # NSLOT-th quartet of a batch, and the slots are summed after the primitive loop
-    nslot = max(1, min(npb, G // nblk)) if (2 * nblk <= G and not col) else 1
-    acc = 1 if (nslot > 1 or col) else (nblk + G - 1) // G
-    smem_group = 2 * NMONO + max(npb * nr * 3 * S, nblk + nab * nc, nslot * nblk)
-    mixed = nblk >= MIXED_MIN_NBLK and (acc <= MIXED_MAX_ACC or col)
-    return dict(la=la, lb=lb, lc=lc, ld=ld, e=e, f=f, nr=nr, rows=rows, cols=cols, S=S,
+    # threads: a column of the block each
+    G = 32 * ((nc + 31) // 32)
+    G = 128 if G > 64 else G
+    bra_lines, ket_lines = HrrSide(la, lb, rows_index), HrrSide(lc, ld, cols_index)
+    # odd row strides: a warp reading a column of rows meets no bank twice
+    ncp, ncdp = nc | 1, ncd | 1
+    # ket pairs per group and round: as many as have columns and a root each, with their HRR
+    # buffers in about 19 KB
+    # (blocks of one or three columns: H threads share a column, each every H-th (quartet, root))
+    H = {1: 8, 3: 2}.get(nc, 1)
+    W = max(1, min(G // (nc * H), 32 // nr, 8)) if G == 32 else 1
+    while W > 1 and W * nab * (ncp + ncdp) > 2400:
+        W -= 1
+    hrr_room = W * nab * (ncp + ncdp)
+    # primitive quartets per ket pair and batch: one stage-1 thread per (ket pair, quartet, root);
+    # the batch's 2-D tables (an odd stride per item) may use the HRR buffers' room
+    si = (3 * S) | 1
+    pb = max(1, min(G // (W * nr), max(hrr_room, 1536 * (G // 32)) // (W * nr * si)))
+    npb = W * pb
+    smem_group = max(npb * nr * si, hrr_room)
+    # the FP32 variant's rule (blocks of some size whose accumulators the first form of this kernel
+    # held in MIXED_MAX_ACC registers a thread of 32 to 128)
+    acc32 = (nblk + (32 if nblk <= 128 else 64 if nblk <= 1024 else 128) - 1) // (32 if nblk <= 128 else 64 if nblk <= 1024 else 128)
+    mixed = nblk >= MIXED_MIN_NBLK and (acc32 <= MIXED_MAX_ACC or (nc >= 16 and na <= COL_MAX_NA))
+    return dict(la=la, lb=lb, lc=lc, ld=ld, e=e, f=f, nr=nr, rows=rows, cols=cols, S=S, SI=si,
                 blk=blk, bra=bra, ket=ket, norm_ab=norm_ab, norm_cd=norm_cd, na=na, nc=nc,
-                nblk=nblk, nab=nab, ncd=ncd, G=G, npb=npb, nslot=nslot, acc=acc,
-                smem_group=smem_group, mixed=mixed, col=col)
-
-
-def _flat_terms(lists):
-    off, flat = [0], []
-    for terms in lists:
-        for src, mono, binom in terms:
-            flat.append(src | (mono << 8) | (binom << 16))
-        off.append(len(flat))
-    return off, flat
+                nblk=nblk, nab=nab, ncd=ncd, ncp=ncp, ncdp=ncdp, G=G, W=W, H=H, pb=pb, npb=npb, nslot=1,
+                acc=max(na, (nblk + G - 1) // G), smem_group=smem_group, mixed=mixed, col=False,
+                bra_side=bra_lines, ket_side=ket_lines)
 
 
 def _arr(vals, fmt=str, per=12):
@@ -192,12 +209,20 @@ def _arr(vals, fmt=str, per=12):
     return "\n".join(lines) if lines else "    0,"
 
 
+def is_lane(X, Y):
+    """Class pairs of small blocks (below the FP32 variant's bound) run a lane-split kernel, the HGP
+    kernel's frame with the lanes' primitive quartets by Rys quadrature: a group of threads per
+    quartet leaves most of them idle (one to thirty block entries) and serialises long contractions.
+    On B200, (ss|ss) of a 60-function molecule (300,949 primitive quartets): group form 342 us."""
+    return class_tables(X, Y)["nblk"] < MIXED_MIN_NBLK
+
+
 def emit_class_pair(X, Y):
+    if is_lane(X, Y):
+        import gen_eri
+        return gen_eri.emit_class_pair(X, Y, rys=True)
     t = class_tables(X, Y)
     tag = tag_of(X, Y)
-    blk = [o[0] | (o[1] << 8) | (o[2] << 16) for o in t["blk"]]
-    boff, bterm = _flat_terms(t["bra"])
-    koff, kterm = _flat_terms(t["ket"])
     smem_block = (128 // t["G"]) * t["smem_group"] * 8
     assert smem_block <= 227 * 1024, (tag, smem_block)
     diag = X == Y
@@ -228,24 +253,27 @@ void launch_rys_bound_{tag}(const PairTab &P, const RysTab &R, int p0, int np, d
                           f"    rys_queue_{tag}<0><<<grid, 128, {smem_block}, s>>>(Q, R);")
         occ_dispatch = (f"    (void)mixed;\n"
                         f"    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_{tag}<0>, 128, {smem_block});")
-    if t["col"]:
-        F1 = t["f"] + 1
-        lines = []
-        for ia, a in enumerate(t["rows"]):
-            lines.append(f"        acc[{ia}] = fma(x[{a[0]}] * y[{a[1]}], z[{a[2]}], acc[{ia}]);")
-        col_code = ("    // stage 2, column mode: acc[row] += x[ax] y[ay] z[az] for the column's table columns\n"
-                    "    template <typename T, typename A>\n"
-                    "    __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {\n"
-                    + "\n".join(lines) + "\n    }")
-        colpow = ", ".join(str(c[0] | (c[1] << 4) | (c[2] << 8)) for c in t["cols"])
-        col_code += f"\n    static constexpr int NCOLS = {t['nc']};"
-        col_tab = f"\n// column components cx | cy << 4 | cz << 8\n__device__ const uint16_t kCol_{tag}[{t['nc']}] = {{ {colpow} }};\n"
-    else:
-        col_code = "    template <typename T, typename A>\n    __device__ __forceinline__ static void col_update(const T *, const T *, const T *, A *) {}"
-        col_tab = ""
+    # stage 2: one block column's row accumulators from its three table columns
+    col_code = ("    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns\n"
+                "    template <typename T, typename A>\n"
+                "    __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {\n"
+                + "\n".join(f"        acc[{ia}] = fma(x[{a[0]}] * y[{a[1]}], z[{a[2]}], acc[{ia}]);"
+                            for ia, a in enumerate(t["rows"])) + "\n    }")
+    colpow = ", ".join(str(c[0] | (c[1] << 4) | (c[2] << 8)) for c in t["cols"])
+    col_tab = f"\n// column components cx | cy << 4 | cz << 8\n__device__ const uint16_t kCol_{tag}[{t['nc']}] = {{ {colpow} }};\n"
+
+    def side_code(name, side, scale, stride):
+        head = (f"    __device__ __forceinline__ static void {name}(const double *__restrict__ in, double x, double y, "
+                f"double z, double nrm, double *__restrict__ out) {{\n")
+        body = "".join(f"        {ln}\n" for ln in side.lines)
+        outs = "".join(f"        out[{r * stride}] = {e}{scale(r)};\n" for r, e in enumerate(side.out))
+        return head + "        (void)x; (void)y; (void)z; (void)nrm;\n" + body + outs + "    }"
+    hrr_code = ("    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms\n" +
+                side_code("bra_hrr", t["bra_side"], lambda r: "", t["ncp"]) + "\n" +
+                side_code("ket_hrr", t["ket_side"], lambda r: f" * (nrm * {t['norm_cd'][r]!r})", 1))
     return f"""// Generated by gen_rys.py -- Rys class ({tag[0]}{tag[1]}|{tag[2]}{tag[3]}).  Do not edit.
-// roots {t['nr']}, block {t['na']} x {t['nc']}, outputs {t['nab']} x {t['ncd']}, group {t['G']} threads,
-// {t['npb']} primitive quartets per batch, {t['nslot']} slot(s), {t['acc']} accumulators per thread, {smem_block} B shared per block{", column mode" if t["col"] else ""}.
+// roots {t['nr']}, block {t['na']} x {t['nc']}, outputs {t['nab']} x {t['ncd']}, group {t['G']} threads, {t['W']} ket pairs a round,
+// {t['pb']} primitive quartets per ket pair and batch, {smem_block} B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {{
@@ -256,41 +284,19 @@ struct C_{tag} {{
     static constexpr int NA = {t['na']}, NC = {t['nc']}, NBLK = {t['nblk']};
     static constexpr int NB = {ncart(t['lb'])}, ND = {ncart(t['ld'])};
     static constexpr int NAB = {t['nab']}, NCD = {t['ncd']};
-    static constexpr int G = {t['G']}, NPB = {t['npb']}, NSLOT = {t['nslot']}, ACC = {t['acc']};
-    static constexpr int S = {t['S']};
+    static constexpr int G = {t['G']}, W = {t['W']}, H = {t['H']}, PB = {t['pb']};
+    static constexpr int S = {t['S']}, SI = {t['SI']}, NCP = {t['ncp']}, NCDP = {t['ncdp']};
     static constexpr int SMEM_GROUP = {t['smem_group']};
-    static constexpr bool COL = {'true' if t['col'] else 'false'};
 {col_code}
+{hrr_code}
 }};
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_{tag}[{len(blk)}] = {{
-{_arr(blk)}
-}};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_{tag}[{len(boff)}] = {{
-{_arr(boff)}
-}};
-__device__ const uint32_t kBraTerm_{tag}[{len(bterm)}] = {{
-{_arr(bterm)}
-}};
-__device__ const uint16_t kKetOff_{tag}[{len(koff)}] = {{
-{_arr(koff)}
-}};
-__device__ const uint32_t kKetTerm_{tag}[{len(kterm)}] = {{
-{_arr(kterm)}
-}};
 __device__ const double kNormAB_{tag}[{len(t['norm_ab'])}] = {{
 {_arr(t['norm_ab'], repr, 4)}
 }};
-__device__ const double kNormCD_{tag}[{len(t['norm_cd'])}] = {{
-{_arr(t['norm_cd'], repr, 4)}
-}};
-
 {col_tab}
 __device__ __forceinline__ RysClassTabs tabs_{tag}() {{
-    return RysClassTabs{{kBlk_{tag}, kBraOff_{tag}, kBraTerm_{tag}, kKetOff_{tag}, kKetTerm_{tag},
-                        kNormAB_{tag}, kNormCD_{tag}, {"kCol_" + tag if t["col"] else "nullptr"}}};
+    return RysClassTabs{{kNormAB_{tag}, kCol_{tag}}};
 }}
 
 template <int MIXED>

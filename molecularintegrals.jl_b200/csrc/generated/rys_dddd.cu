@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (dd|dd).  Do not edit.
-// roots 5, block 31 x 31, outputs 36 x 36, group 32 threads,
-// 6 primitive quartets per batch, 1 slot(s), 1 accumulators per thread, 73280 B shared per block, column mode.
+// roots 5, block 31 x 31, outputs 36 x 36, group 32 threads, 1 ket pairs a round,
+// 6 primitive quartets per ket pair and batch, 78336 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,11 +11,10 @@ struct C_dddd {
     static constexpr int NA = 31, NC = 31, NBLK = 961;
     static constexpr int NB = 6, ND = 6;
     static constexpr int NAB = 36, NCD = 36;
-    static constexpr int G = 32, NPB = 6, NSLOT = 1, ACC = 1;
-    static constexpr int S = 25;
-    static constexpr int SMEM_GROUP = 2290;
-    static constexpr bool COL = true;
-    // stage 2, column mode: acc[row] += x[ax] y[ay] z[az] for the column's table columns
+    static constexpr int G = 32, W = 1, H = 1, PB = 6;
+    static constexpr int S = 25, SI = 75, NCP = 31, NCDP = 37;
+    static constexpr int SMEM_GROUP = 2448;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
     __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
         acc[0] = fma(x[2] * y[0], z[0], acc[0]);
@@ -50,132 +49,245 @@ struct C_dddd {
         acc[29] = fma(x[0] * y[1], z[3], acc[29]);
         acc[30] = fma(x[0] * y[0], z[4], acc[30]);
     }
-    static constexpr int NCOLS = 31;
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[6], in[16]);
+        const double h1 = fma(x, in[0], in[6]);
+        const double h2 = fma(x, h1, h0);
+        const double h3 = fma(y, in[6], in[17]);
+        const double h4 = fma(y, in[0], in[7]);
+        const double h5 = fma(x, h4, h3);
+        const double h6 = fma(z, in[6], in[18]);
+        const double h7 = fma(z, in[0], in[8]);
+        const double h8 = fma(x, h7, h6);
+        const double h9 = fma(y, in[7], in[19]);
+        const double h10 = fma(y, h4, h9);
+        const double h11 = fma(z, in[7], in[20]);
+        const double h12 = fma(y, h7, h11);
+        const double h13 = fma(z, in[8], in[21]);
+        const double h14 = fma(z, h7, h13);
+        const double h15 = fma(x, in[7], in[17]);
+        const double h16 = fma(x, in[1], in[7]);
+        const double h17 = fma(x, h16, h15);
+        const double h18 = fma(y, in[1], in[9]);
+        const double h19 = fma(x, h18, h9);
+        const double h20 = fma(z, in[1], in[11]);
+        const double h21 = fma(x, h20, h11);
+        const double h22 = fma(y, in[9], in[22]);
+        const double h23 = fma(y, h18, h22);
+        const double h24 = fma(z, in[9], in[23]);
+        const double h25 = fma(y, h20, h24);
+        const double h26 = fma(z, in[11], in[24]);
+        const double h27 = fma(z, h20, h26);
+        const double h28 = fma(x, in[8], in[18]);
+        const double h29 = fma(x, in[2], in[8]);
+        const double h30 = fma(x, h29, h28);
+        const double h31 = fma(y, in[8], in[20]);
+        const double h32 = fma(y, in[2], in[11]);
+        const double h33 = fma(x, h32, h31);
+        const double h34 = fma(z, in[2], in[10]);
+        const double h35 = fma(x, h34, h13);
+        const double h36 = fma(y, in[11], in[23]);
+        const double h37 = fma(y, h32, h36);
+        const double h38 = fma(y, h34, h26);
+        const double h39 = fma(z, in[10], in[25]);
+        const double h40 = fma(z, h34, h39);
+        const double h41 = fma(x, in[9], in[19]);
+        const double h42 = fma(x, in[3], in[9]);
+        const double h43 = fma(x, h42, h41);
+        const double h44 = fma(y, in[3], in[12]);
+        const double h45 = fma(x, h44, h22);
+        const double h46 = fma(z, in[3], in[13]);
+        const double h47 = fma(x, h46, h24);
+        const double h48 = fma(y, in[12], in[26]);
+        const double h49 = fma(y, h44, h48);
+        const double h50 = fma(z, in[12], in[27]);
+        const double h51 = fma(y, h46, h50);
+        const double h52 = fma(z, in[13], in[28]);
+        const double h53 = fma(z, h46, h52);
+        const double h54 = fma(x, in[11], in[20]);
+        const double h55 = fma(x, in[4], in[11]);
+        const double h56 = fma(x, h55, h54);
+        const double h57 = fma(y, in[4], in[13]);
+        const double h58 = fma(x, h57, h36);
+        const double h59 = fma(z, in[4], in[14]);
+        const double h60 = fma(x, h59, h26);
+        const double h61 = fma(y, in[13], in[27]);
+        const double h62 = fma(y, h57, h61);
+        const double h63 = fma(y, h59, h52);
+        const double h64 = fma(z, in[14], in[29]);
+        const double h65 = fma(z, h59, h64);
+        const double h66 = fma(x, in[10], in[21]);
+        const double h67 = fma(x, in[5], in[10]);
+        const double h68 = fma(x, h67, h66);
+        const double h69 = fma(y, in[10], in[24]);
+        const double h70 = fma(y, in[5], in[14]);
+        const double h71 = fma(x, h70, h69);
+        const double h72 = fma(z, in[5], in[15]);
+        const double h73 = fma(x, h72, h39);
+        const double h74 = fma(y, in[14], in[28]);
+        const double h75 = fma(y, h70, h74);
+        const double h76 = fma(y, h72, h64);
+        const double h77 = fma(z, in[15], in[30]);
+        const double h78 = fma(z, h72, h77);
+        out[0] = h2;
+        out[31] = h5;
+        out[62] = h8;
+        out[93] = h10;
+        out[124] = h12;
+        out[155] = h14;
+        out[186] = h17;
+        out[217] = h19;
+        out[248] = h21;
+        out[279] = h23;
+        out[310] = h25;
+        out[341] = h27;
+        out[372] = h30;
+        out[403] = h33;
+        out[434] = h35;
+        out[465] = h37;
+        out[496] = h38;
+        out[527] = h40;
+        out[558] = h43;
+        out[589] = h45;
+        out[620] = h47;
+        out[651] = h49;
+        out[682] = h51;
+        out[713] = h53;
+        out[744] = h56;
+        out[775] = h58;
+        out[806] = h60;
+        out[837] = h62;
+        out[868] = h63;
+        out[899] = h65;
+        out[930] = h68;
+        out[961] = h71;
+        out[992] = h73;
+        out[1023] = h75;
+        out[1054] = h76;
+        out[1085] = h78;
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[6], in[16]);
+        const double h1 = fma(x, in[0], in[6]);
+        const double h2 = fma(x, h1, h0);
+        const double h3 = fma(y, in[6], in[17]);
+        const double h4 = fma(y, in[0], in[7]);
+        const double h5 = fma(x, h4, h3);
+        const double h6 = fma(z, in[6], in[18]);
+        const double h7 = fma(z, in[0], in[8]);
+        const double h8 = fma(x, h7, h6);
+        const double h9 = fma(y, in[7], in[19]);
+        const double h10 = fma(y, h4, h9);
+        const double h11 = fma(z, in[7], in[20]);
+        const double h12 = fma(y, h7, h11);
+        const double h13 = fma(z, in[8], in[21]);
+        const double h14 = fma(z, h7, h13);
+        const double h15 = fma(x, in[7], in[17]);
+        const double h16 = fma(x, in[1], in[7]);
+        const double h17 = fma(x, h16, h15);
+        const double h18 = fma(y, in[1], in[9]);
+        const double h19 = fma(x, h18, h9);
+        const double h20 = fma(z, in[1], in[11]);
+        const double h21 = fma(x, h20, h11);
+        const double h22 = fma(y, in[9], in[22]);
+        const double h23 = fma(y, h18, h22);
+        const double h24 = fma(z, in[9], in[23]);
+        const double h25 = fma(y, h20, h24);
+        const double h26 = fma(z, in[11], in[24]);
+        const double h27 = fma(z, h20, h26);
+        const double h28 = fma(x, in[8], in[18]);
+        const double h29 = fma(x, in[2], in[8]);
+        const double h30 = fma(x, h29, h28);
+        const double h31 = fma(y, in[8], in[20]);
+        const double h32 = fma(y, in[2], in[11]);
+        const double h33 = fma(x, h32, h31);
+        const double h34 = fma(z, in[2], in[10]);
+        const double h35 = fma(x, h34, h13);
+        const double h36 = fma(y, in[11], in[23]);
+        const double h37 = fma(y, h32, h36);
+        const double h38 = fma(y, h34, h26);
+        const double h39 = fma(z, in[10], in[25]);
+        const double h40 = fma(z, h34, h39);
+        const double h41 = fma(x, in[9], in[19]);
+        const double h42 = fma(x, in[3], in[9]);
+        const double h43 = fma(x, h42, h41);
+        const double h44 = fma(y, in[3], in[12]);
+        const double h45 = fma(x, h44, h22);
+        const double h46 = fma(z, in[3], in[13]);
+        const double h47 = fma(x, h46, h24);
+        const double h48 = fma(y, in[12], in[26]);
+        const double h49 = fma(y, h44, h48);
+        const double h50 = fma(z, in[12], in[27]);
+        const double h51 = fma(y, h46, h50);
+        const double h52 = fma(z, in[13], in[28]);
+        const double h53 = fma(z, h46, h52);
+        const double h54 = fma(x, in[11], in[20]);
+        const double h55 = fma(x, in[4], in[11]);
+        const double h56 = fma(x, h55, h54);
+        const double h57 = fma(y, in[4], in[13]);
+        const double h58 = fma(x, h57, h36);
+        const double h59 = fma(z, in[4], in[14]);
+        const double h60 = fma(x, h59, h26);
+        const double h61 = fma(y, in[13], in[27]);
+        const double h62 = fma(y, h57, h61);
+        const double h63 = fma(y, h59, h52);
+        const double h64 = fma(z, in[14], in[29]);
+        const double h65 = fma(z, h59, h64);
+        const double h66 = fma(x, in[10], in[21]);
+        const double h67 = fma(x, in[5], in[10]);
+        const double h68 = fma(x, h67, h66);
+        const double h69 = fma(y, in[10], in[24]);
+        const double h70 = fma(y, in[5], in[14]);
+        const double h71 = fma(x, h70, h69);
+        const double h72 = fma(z, in[5], in[15]);
+        const double h73 = fma(x, h72, h39);
+        const double h74 = fma(y, in[14], in[28]);
+        const double h75 = fma(y, h70, h74);
+        const double h76 = fma(y, h72, h64);
+        const double h77 = fma(z, in[15], in[30]);
+        const double h78 = fma(z, h72, h77);
+        out[0] = h2 * (nrm * 0.3333333333333334);
+        out[1] = h5 * (nrm * 0.5773502691896258);
+        out[2] = h8 * (nrm * 0.5773502691896258);
+        out[3] = h10 * (nrm * 0.3333333333333334);
+        out[4] = h12 * (nrm * 0.5773502691896258);
+        out[5] = h14 * (nrm * 0.3333333333333334);
+        out[6] = h17 * (nrm * 0.5773502691896258);
+        out[7] = h19 * (nrm * 1.0);
+        out[8] = h21 * (nrm * 1.0);
+        out[9] = h23 * (nrm * 0.5773502691896258);
+        out[10] = h25 * (nrm * 1.0);
+        out[11] = h27 * (nrm * 0.5773502691896258);
+        out[12] = h30 * (nrm * 0.5773502691896258);
+        out[13] = h33 * (nrm * 1.0);
+        out[14] = h35 * (nrm * 1.0);
+        out[15] = h37 * (nrm * 0.5773502691896258);
+        out[16] = h38 * (nrm * 1.0);
+        out[17] = h40 * (nrm * 0.5773502691896258);
+        out[18] = h43 * (nrm * 0.3333333333333334);
+        out[19] = h45 * (nrm * 0.5773502691896258);
+        out[20] = h47 * (nrm * 0.5773502691896258);
+        out[21] = h49 * (nrm * 0.3333333333333334);
+        out[22] = h51 * (nrm * 0.5773502691896258);
+        out[23] = h53 * (nrm * 0.3333333333333334);
+        out[24] = h56 * (nrm * 0.5773502691896258);
+        out[25] = h58 * (nrm * 1.0);
+        out[26] = h60 * (nrm * 1.0);
+        out[27] = h62 * (nrm * 0.5773502691896258);
+        out[28] = h63 * (nrm * 1.0);
+        out[29] = h65 * (nrm * 0.5773502691896258);
+        out[30] = h68 * (nrm * 0.3333333333333334);
+        out[31] = h71 * (nrm * 0.5773502691896258);
+        out[32] = h73 * (nrm * 0.5773502691896258);
+        out[33] = h75 * (nrm * 0.3333333333333334);
+        out[34] = h76 * (nrm * 0.5773502691896258);
+        out[35] = h78 * (nrm * 0.3333333333333334);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_dddd[961] = {
-    12, 267, 65547, 522, 65802, 131082, 13, 268, 65548, 523, 131083, 65803,
-    778, 66058, 131338, 196618, 14, 269, 65549, 524, 65804, 131084, 779, 66059,
-    131339, 196619, 1034, 66314, 131594, 196874, 262154, 1287, 1542, 66822, 1797, 67077,
-    132357, 1288, 1543, 66823, 1798, 132358, 67078, 2053, 67333, 132613, 197893, 1289,
-    1544, 66824, 1799, 67079, 132359, 2054, 67334, 132614, 197894, 2309, 67589, 132869,
-    198149, 263429, 327687, 327942, 393222, 328197, 393477, 458757, 327688, 327943, 393223, 328198,
-    458758, 393478, 328453, 393733, 459013, 524293, 327689, 327944, 393224, 328199, 393479, 458759,
-    328454, 393734, 459014, 524294, 328709, 393989, 459269, 524549, 589829, 2562, 2817, 68097,
-    3072, 68352, 133632, 2563, 2818, 68098, 3073, 133633, 68353, 3328, 68608, 133888,
-    199168, 2564, 2819, 68099, 3074, 68354, 133634, 3329, 68609, 133889, 199169, 3584,
-    68864, 134144, 199424, 264704, 328962, 329217, 394497, 329472, 394752, 460032, 328963, 329218,
-    394498, 329473, 460033, 394753, 329728, 395008, 460288, 525568, 328964, 329219, 394499, 329474,
-    394754, 460034, 329729, 395009, 460289, 525569, 329984, 395264, 460544, 525824, 591104, 655362,
-    655617, 720897, 655872, 721152, 786432, 655363, 655618, 720898, 655873, 786433, 721153, 656128,
-    721408, 786688, 851968, 655364, 655619, 720899, 655874, 721154, 786434, 656129, 721409, 786689,
-    851969, 656384, 721664, 786944, 852224, 917504, 17, 272, 65552, 527, 65807, 131087,
-    18, 273, 65553, 528, 131088, 65808, 783, 66063, 131343, 196623, 19, 274,
-    65554, 529, 65809, 131089, 784, 66064, 131344, 196624, 1039, 66319, 131599, 196879,
-    262159, 1292, 1547, 66827, 1802, 67082, 132362, 1293, 1548, 66828, 1803, 132363,
-    67083, 2058, 67338, 132618, 197898, 1294, 1549, 66829, 1804, 67084, 132364, 2059,
-    67339, 132619, 197899, 2314, 67594, 132874, 198154, 263434, 327692, 327947, 393227, 328202,
-    393482, 458762, 327693, 327948, 393228, 328203, 458763, 393483, 328458, 393738, 459018, 524298,
-    327694, 327949, 393229, 328204, 393484, 458764, 328459, 393739, 459019, 524299, 328714, 393994,
-    459274, 524554, 589834, 2567, 2822, 68102, 3077, 68357, 133637, 2568, 2823, 68103,
-    3078, 133638, 68358, 3333, 68613, 133893, 199173, 2569, 2824, 68104, 3079, 68359,
-    133639, 3334, 68614, 133894, 199174, 3589, 68869, 134149, 199429, 264709, 655367, 655622,
-    720902, 655877, 721157, 786437, 655368, 655623, 720903, 655878, 786438, 721158, 656133, 721413,
-    786693, 851973, 655369, 655624, 720904, 655879, 721159, 786439, 656134, 721414, 786694, 851974,
-    656389, 721669, 786949, 852229, 917509, 328967, 329222, 394502, 329477, 394757, 460037, 328968,
-    329223, 394503, 329478, 460038, 394758, 329733, 395013, 460293, 525573, 328969, 329224, 394504,
-    329479, 394759, 460039, 329734, 395014, 460294, 525574, 329989, 395269, 460549, 525829, 591109,
-    3842, 4097, 69377, 4352, 69632, 134912, 3843, 4098, 69378, 4353, 134913, 69633,
-    4608, 69888, 135168, 200448, 3844, 4099, 69379, 4354, 69634, 134914, 4609, 69889,
-    135169, 200449, 4864, 70144, 135424, 200704, 265984, 330242, 330497, 395777, 330752, 396032,
-    461312, 330243, 330498, 395778, 330753, 461313, 396033, 331008, 396288, 461568, 526848, 330244,
-    330499, 395779, 330754, 396034, 461314, 331009, 396289, 461569, 526849, 331264, 396544, 461824,
-    527104, 592384, 656642, 656897, 722177, 657152, 722432, 787712, 656643, 656898, 722178, 657153,
-    787713, 722433, 657408, 722688, 787968, 853248, 656644, 656899, 722179, 657154, 722434, 787714,
-    657409, 722689, 787969, 853249, 657664, 722944, 788224, 853504, 918784, 983042, 983297, 1048577,
-    983552, 1048832, 1114112, 983043, 983298, 1048578, 983553, 1114113, 1048833, 983808, 1049088, 1114368,
-    1179648, 983044, 983299, 1048579, 983554, 1048834, 1114114, 983809, 1049089, 1114369, 1179649, 984064,
-    1049344, 1114624, 1179904, 1245184, 22, 277, 65557, 532, 65812, 131092, 23, 278,
-    65558, 533, 131093, 65813, 788, 66068, 131348, 196628, 24, 279, 65559, 534,
-    65814, 131094, 789, 66069, 131349, 196629, 1044, 66324, 131604, 196884, 262164, 1297,
-    1552, 66832, 1807, 67087, 132367, 1298, 1553, 66833, 1808, 132368, 67088, 2063,
-    67343, 132623, 197903, 1299, 1554, 66834, 1809, 67089, 132369, 2064, 67344, 132624,
-    197904, 2319, 67599, 132879, 198159, 263439, 327697, 327952, 393232, 328207, 393487, 458767,
-    327698, 327953, 393233, 328208, 458768, 393488, 328463, 393743, 459023, 524303, 327699, 327954,
-    393234, 328209, 393489, 458769, 328464, 393744, 459024, 524304, 328719, 393999, 459279, 524559,
-    589839, 2572, 2827, 68107, 3082, 68362, 133642, 2573, 2828, 68108, 3083, 133643,
-    68363, 3338, 68618, 133898, 199178, 2574, 2829, 68109, 3084, 68364, 133644, 3339,
-    68619, 133899, 199179, 3594, 68874, 134154, 199434, 264714, 328972, 329227, 394507, 329482,
-    394762, 460042, 328973, 329228, 394508, 329483, 460043, 394763, 329738, 395018, 460298, 525578,
-    328974, 329229, 394509, 329484, 394764, 460044, 329739, 395019, 460299, 525579, 329994, 395274,
-    460554, 525834, 591114, 655372, 655627, 720907, 655882, 721162, 786442, 655373, 655628, 720908,
-    655883, 786443, 721163, 656138, 721418, 786698, 851978, 655374, 655629, 720909, 655884, 721164,
-    786444, 656139, 721419, 786699, 851979, 656394, 721674, 786954, 852234, 917514, 3847, 4102,
-    69382, 4357, 69637, 134917, 3848, 4103, 69383, 4358, 134918, 69638, 4613, 69893,
-    135173, 200453, 3849, 4104, 69384, 4359, 69639, 134919, 4614, 69894, 135174, 200454,
-    4869, 70149, 135429, 200709, 265989, 330247, 330502, 395782, 330757, 396037, 461317, 330248,
-    330503, 395783, 330758, 461318, 396038, 331013, 396293, 461573, 526853, 330249, 330504, 395784,
-    330759, 396039, 461319, 331014, 396294, 461574, 526854, 331269, 396549, 461829, 527109, 592389,
-    656647, 656902, 722182, 657157, 722437, 787717, 656648, 656903, 722183, 657158, 787718, 722438,
-    657413, 722693, 787973, 853253, 656649, 656904, 722184, 657159, 722439, 787719, 657414, 722694,
-    787974, 853254, 657669, 722949, 788229, 853509, 918789, 983047, 983302, 1048582, 983557, 1048837,
-    1114117, 983048, 983303, 1048583, 983558, 1114118, 1048838, 983813, 1049093, 1114373, 1179653, 983049,
-    983304, 1048584, 983559, 1048839, 1114119, 983814, 1049094, 1114374, 1179654, 984069, 1049349, 1114629,
-    1179909, 1245189, 5122, 5377, 70657, 5632, 70912, 136192, 5123, 5378, 70658, 5633,
-    136193, 70913, 5888, 71168, 136448, 201728, 5124, 5379, 70659, 5634, 70914, 136194,
-    5889, 71169, 136449, 201729, 6144, 71424, 136704, 201984, 267264, 331522, 331777, 397057,
-    332032, 397312, 462592, 331523, 331778, 397058, 332033, 462593, 397313, 332288, 397568, 462848,
-    528128, 331524, 331779, 397059, 332034, 397314, 462594, 332289, 397569, 462849, 528129, 332544,
-    397824, 463104, 528384, 593664, 657922, 658177, 723457, 658432, 723712, 788992, 657923, 658178,
-    723458, 658433, 788993, 723713, 658688, 723968, 789248, 854528, 657924, 658179, 723459, 658434,
-    723714, 788994, 658689, 723969, 789249, 854529, 658944, 724224, 789504, 854784, 920064, 984322,
-    984577, 1049857, 984832, 1050112, 1115392, 984323, 984578, 1049858, 984833, 1115393, 1050113, 985088,
-    1050368, 1115648, 1180928, 984324, 984579, 1049859, 984834, 1050114, 1115394, 985089, 1050369, 1115649,
-    1180929, 985344, 1050624, 1115904, 1181184, 1246464, 1310722, 1310977, 1376257, 1311232, 1376512, 1441792,
-    1310723, 1310978, 1376258, 1311233, 1441793, 1376513, 1311488, 1376768, 1442048, 1507328, 1310724, 1310979,
-    1376259, 1311234, 1376514, 1441794, 1311489, 1376769, 1442049, 1507329, 1311744, 1377024, 1442304, 1507584,
-    1572864,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_dddd[37] = {
-    0, 3, 7, 11, 14, 18, 21, 24, 28, 32, 35, 39,
-    42, 45, 49, 53, 56, 60, 63, 66, 70, 74, 77, 81,
-    84, 87, 91, 95, 98, 102, 105, 108, 112, 116, 119, 123,
-    126,
-};
-__device__ const uint32_t kBraTerm_dddd[126] = {
-    66560, 131334, 65552, 66816, 65799, 66054, 65553, 67072, 65800, 66310, 65554, 67328,
-    131591, 65555, 67584, 66056, 66311, 65556, 67840, 131848, 65557, 66561, 131335, 65553,
-    66817, 65801, 66055, 65555, 67073, 65803, 66311, 65556, 67329, 131593, 65558, 67585,
-    66059, 66313, 65559, 67841, 131851, 65560, 66562, 131336, 65554, 66818, 65803, 66056,
-    65556, 67074, 65802, 66312, 65557, 67330, 131595, 65559, 67586, 66058, 66315, 65560,
-    67842, 131850, 65561, 66563, 131337, 65555, 66819, 65804, 66057, 65558, 67075, 65805,
-    66313, 65559, 67331, 131596, 65562, 67587, 66061, 66316, 65563, 67843, 131853, 65564,
-    66564, 131339, 65556, 66820, 65805, 66059, 65559, 67076, 65806, 66315, 65560, 67332,
-    131597, 65563, 67588, 66062, 66317, 65564, 67844, 131854, 65565, 66565, 131338, 65557,
-    66821, 65806, 66058, 65560, 67077, 65807, 66314, 65561, 67333, 131598, 65564, 67589,
-    66063, 66318, 65565, 67845, 131855, 65566,
-};
-__device__ const uint16_t kKetOff_dddd[37] = {
-    0, 3, 7, 11, 14, 18, 21, 24, 28, 32, 35, 39,
-    42, 45, 49, 53, 56, 60, 63, 66, 70, 74, 77, 81,
-    84, 87, 91, 95, 98, 102, 105, 108, 112, 116, 119, 123,
-    126,
-};
-__device__ const uint32_t kKetTerm_dddd[126] = {
-    66560, 131334, 65552, 66816, 65799, 66054, 65553, 67072, 65800, 66310, 65554, 67328,
-    131591, 65555, 67584, 66056, 66311, 65556, 67840, 131848, 65557, 66561, 131335, 65553,
-    66817, 65801, 66055, 65555, 67073, 65803, 66311, 65556, 67329, 131593, 65558, 67585,
-    66059, 66313, 65559, 67841, 131851, 65560, 66562, 131336, 65554, 66818, 65803, 66056,
-    65556, 67074, 65802, 66312, 65557, 67330, 131595, 65559, 67586, 66058, 66315, 65560,
-    67842, 131850, 65561, 66563, 131337, 65555, 66819, 65804, 66057, 65558, 67075, 65805,
-    66313, 65559, 67331, 131596, 65562, 67587, 66061, 66316, 65563, 67843, 131853, 65564,
-    66564, 131339, 65556, 66820, 65805, 66059, 65559, 67076, 65806, 66315, 65560, 67332,
-    131597, 65563, 67588, 66062, 66317, 65564, 67844, 131854, 65565, 66565, 131338, 65557,
-    66821, 65806, 66058, 65560, 67077, 65807, 66314, 65561, 67333, 131598, 65564, 67589,
-    66063, 66318, 65565, 67845, 131855, 65566,
-};
 __device__ const double kNormAB_dddd[36] = {
     0.3333333333333334, 0.5773502691896258, 0.5773502691896258, 0.3333333333333334,
     0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 1.0,
@@ -187,25 +299,12 @@ __device__ const double kNormAB_dddd[36] = {
     1.0, 0.5773502691896258, 0.3333333333333334, 0.5773502691896258,
     0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 0.3333333333333334,
 };
-__device__ const double kNormCD_dddd[36] = {
-    0.3333333333333334, 0.5773502691896258, 0.5773502691896258, 0.3333333333333334,
-    0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 1.0,
-    1.0, 0.5773502691896258, 1.0, 0.5773502691896258,
-    0.5773502691896258, 1.0, 1.0, 0.5773502691896258,
-    1.0, 0.5773502691896258, 0.3333333333333334, 0.5773502691896258,
-    0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 0.3333333333333334,
-    0.5773502691896258, 1.0, 1.0, 0.5773502691896258,
-    1.0, 0.5773502691896258, 0.3333333333333334, 0.5773502691896258,
-    0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 0.3333333333333334,
-};
-
 
 // column components cx | cy << 4 | cz << 8
 __device__ const uint16_t kCol_dddd[31] = { 2, 17, 257, 32, 272, 512, 3, 18, 258, 33, 513, 273, 48, 288, 528, 768, 4, 19, 259, 34, 274, 514, 49, 289, 529, 769, 64, 304, 544, 784, 1024 };
 
 __device__ __forceinline__ RysClassTabs tabs_dddd() {
-    return RysClassTabs{kBlk_dddd, kBraOff_dddd, kBraTerm_dddd, kKetOff_dddd, kKetTerm_dddd,
-                        kNormAB_dddd, kNormCD_dddd, kCol_dddd};
+    return RysClassTabs{kNormAB_dddd, kCol_dddd};
 }
 
 template <int MIXED>
@@ -223,9 +322,9 @@ static void rys_prepare_dddd() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_dddd<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 73280);
-        cudaFuncSetAttribute(rys_queue_dddd<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 73280);
-        cudaFuncSetAttribute(rys_bound_kernel_dddd, cudaFuncAttributeMaxDynamicSharedMemorySize, 73280);
+        cudaFuncSetAttribute(rys_queue_dddd<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 78336);
+        cudaFuncSetAttribute(rys_queue_dddd<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 78336);
+        cudaFuncSetAttribute(rys_bound_kernel_dddd, cudaFuncAttributeMaxDynamicSharedMemorySize, 78336);
         done[dev] = true;
     }
 }
@@ -236,16 +335,16 @@ void launch_rys_dddd(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_dddd();
     constexpr int ng = 128 / C_dddd::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_dddd<1><<<grid, 128, 73280, s>>>(Q, R);
-    else rys_queue_dddd<0><<<grid, 128, 73280, s>>>(Q, R);
+    if (mixed) rys_queue_dddd<1><<<grid, 128, 78336, s>>>(Q, R);
+    else rys_queue_dddd<0><<<grid, 128, 78336, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_dddd(int mixed) {
     rys_prepare_dddd();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dddd<1>, 128, 73280);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dddd<0>, 128, 73280);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dddd<1>, 128, 78336);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dddd<0>, 128, 78336);
     return n;
 }
 
@@ -254,7 +353,7 @@ void launch_rys_bound_dddd(const PairTab &P, const RysTab &R, int p0, int np, do
     if (np <= 0) return;
     rys_prepare_dddd();
     constexpr int ng = 128 / C_dddd::G;
-    rys_bound_kernel_dddd<<<(np + ng - 1) / ng, 128, 73280, s>>>(P, R, p0, np, pbound, qout, full);
+    rys_bound_kernel_dddd<<<(np + ng - 1) / ng, 128, 78336, s>>>(P, R, p0, np, pbound, qout, full);
 }
 
 }  // namespace molints

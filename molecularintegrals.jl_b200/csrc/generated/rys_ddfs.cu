@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (dd|fs).  Do not edit.
-// roots 4, block 31 x 10, outputs 36 x 10, group 64 threads,
-// 16 primitive quartets per batch, 1 slot(s), 5 accumulators per thread, 62080 B shared per block.
+// roots 4, block 31 x 10, outputs 36 x 10, group 32 threads, 3 ket pairs a round,
+// 2 primitive quartets per ket pair and batch, 76032 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,69 +11,178 @@ struct C_ddfs {
     static constexpr int NA = 31, NC = 10, NBLK = 310;
     static constexpr int NB = 6, ND = 1;
     static constexpr int NAB = 36, NCD = 10;
-    static constexpr int G = 64, NPB = 16, NSLOT = 1, ACC = 5;
-    static constexpr int S = 20;
-    static constexpr int SMEM_GROUP = 3880;
-    static constexpr bool COL = false;
+    static constexpr int G = 32, W = 3, H = 1, PB = 2;
+    static constexpr int S = 20, SI = 61, NCP = 11, NCDP = 11;
+    static constexpr int SMEM_GROUP = 2376;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
-    __device__ __forceinline__ static void col_update(const T *, const T *, const T *, A *) {}
+    __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
+        acc[0] = fma(x[2] * y[0], z[0], acc[0]);
+        acc[1] = fma(x[1] * y[1], z[0], acc[1]);
+        acc[2] = fma(x[1] * y[0], z[1], acc[2]);
+        acc[3] = fma(x[0] * y[2], z[0], acc[3]);
+        acc[4] = fma(x[0] * y[1], z[1], acc[4]);
+        acc[5] = fma(x[0] * y[0], z[2], acc[5]);
+        acc[6] = fma(x[3] * y[0], z[0], acc[6]);
+        acc[7] = fma(x[2] * y[1], z[0], acc[7]);
+        acc[8] = fma(x[2] * y[0], z[1], acc[8]);
+        acc[9] = fma(x[1] * y[2], z[0], acc[9]);
+        acc[10] = fma(x[1] * y[0], z[2], acc[10]);
+        acc[11] = fma(x[1] * y[1], z[1], acc[11]);
+        acc[12] = fma(x[0] * y[3], z[0], acc[12]);
+        acc[13] = fma(x[0] * y[2], z[1], acc[13]);
+        acc[14] = fma(x[0] * y[1], z[2], acc[14]);
+        acc[15] = fma(x[0] * y[0], z[3], acc[15]);
+        acc[16] = fma(x[4] * y[0], z[0], acc[16]);
+        acc[17] = fma(x[3] * y[1], z[0], acc[17]);
+        acc[18] = fma(x[3] * y[0], z[1], acc[18]);
+        acc[19] = fma(x[2] * y[2], z[0], acc[19]);
+        acc[20] = fma(x[2] * y[1], z[1], acc[20]);
+        acc[21] = fma(x[2] * y[0], z[2], acc[21]);
+        acc[22] = fma(x[1] * y[3], z[0], acc[22]);
+        acc[23] = fma(x[1] * y[2], z[1], acc[23]);
+        acc[24] = fma(x[1] * y[1], z[2], acc[24]);
+        acc[25] = fma(x[1] * y[0], z[3], acc[25]);
+        acc[26] = fma(x[0] * y[4], z[0], acc[26]);
+        acc[27] = fma(x[0] * y[3], z[1], acc[27]);
+        acc[28] = fma(x[0] * y[2], z[2], acc[28]);
+        acc[29] = fma(x[0] * y[1], z[3], acc[29]);
+        acc[30] = fma(x[0] * y[0], z[4], acc[30]);
+    }
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[6], in[16]);
+        const double h1 = fma(x, in[0], in[6]);
+        const double h2 = fma(x, h1, h0);
+        const double h3 = fma(y, in[6], in[17]);
+        const double h4 = fma(y, in[0], in[7]);
+        const double h5 = fma(x, h4, h3);
+        const double h6 = fma(z, in[6], in[18]);
+        const double h7 = fma(z, in[0], in[8]);
+        const double h8 = fma(x, h7, h6);
+        const double h9 = fma(y, in[7], in[19]);
+        const double h10 = fma(y, h4, h9);
+        const double h11 = fma(z, in[7], in[20]);
+        const double h12 = fma(y, h7, h11);
+        const double h13 = fma(z, in[8], in[21]);
+        const double h14 = fma(z, h7, h13);
+        const double h15 = fma(x, in[7], in[17]);
+        const double h16 = fma(x, in[1], in[7]);
+        const double h17 = fma(x, h16, h15);
+        const double h18 = fma(y, in[1], in[9]);
+        const double h19 = fma(x, h18, h9);
+        const double h20 = fma(z, in[1], in[11]);
+        const double h21 = fma(x, h20, h11);
+        const double h22 = fma(y, in[9], in[22]);
+        const double h23 = fma(y, h18, h22);
+        const double h24 = fma(z, in[9], in[23]);
+        const double h25 = fma(y, h20, h24);
+        const double h26 = fma(z, in[11], in[24]);
+        const double h27 = fma(z, h20, h26);
+        const double h28 = fma(x, in[8], in[18]);
+        const double h29 = fma(x, in[2], in[8]);
+        const double h30 = fma(x, h29, h28);
+        const double h31 = fma(y, in[8], in[20]);
+        const double h32 = fma(y, in[2], in[11]);
+        const double h33 = fma(x, h32, h31);
+        const double h34 = fma(z, in[2], in[10]);
+        const double h35 = fma(x, h34, h13);
+        const double h36 = fma(y, in[11], in[23]);
+        const double h37 = fma(y, h32, h36);
+        const double h38 = fma(y, h34, h26);
+        const double h39 = fma(z, in[10], in[25]);
+        const double h40 = fma(z, h34, h39);
+        const double h41 = fma(x, in[9], in[19]);
+        const double h42 = fma(x, in[3], in[9]);
+        const double h43 = fma(x, h42, h41);
+        const double h44 = fma(y, in[3], in[12]);
+        const double h45 = fma(x, h44, h22);
+        const double h46 = fma(z, in[3], in[13]);
+        const double h47 = fma(x, h46, h24);
+        const double h48 = fma(y, in[12], in[26]);
+        const double h49 = fma(y, h44, h48);
+        const double h50 = fma(z, in[12], in[27]);
+        const double h51 = fma(y, h46, h50);
+        const double h52 = fma(z, in[13], in[28]);
+        const double h53 = fma(z, h46, h52);
+        const double h54 = fma(x, in[11], in[20]);
+        const double h55 = fma(x, in[4], in[11]);
+        const double h56 = fma(x, h55, h54);
+        const double h57 = fma(y, in[4], in[13]);
+        const double h58 = fma(x, h57, h36);
+        const double h59 = fma(z, in[4], in[14]);
+        const double h60 = fma(x, h59, h26);
+        const double h61 = fma(y, in[13], in[27]);
+        const double h62 = fma(y, h57, h61);
+        const double h63 = fma(y, h59, h52);
+        const double h64 = fma(z, in[14], in[29]);
+        const double h65 = fma(z, h59, h64);
+        const double h66 = fma(x, in[10], in[21]);
+        const double h67 = fma(x, in[5], in[10]);
+        const double h68 = fma(x, h67, h66);
+        const double h69 = fma(y, in[10], in[24]);
+        const double h70 = fma(y, in[5], in[14]);
+        const double h71 = fma(x, h70, h69);
+        const double h72 = fma(z, in[5], in[15]);
+        const double h73 = fma(x, h72, h39);
+        const double h74 = fma(y, in[14], in[28]);
+        const double h75 = fma(y, h70, h74);
+        const double h76 = fma(y, h72, h64);
+        const double h77 = fma(z, in[15], in[30]);
+        const double h78 = fma(z, h72, h77);
+        out[0] = h2;
+        out[11] = h5;
+        out[22] = h8;
+        out[33] = h10;
+        out[44] = h12;
+        out[55] = h14;
+        out[66] = h17;
+        out[77] = h19;
+        out[88] = h21;
+        out[99] = h23;
+        out[110] = h25;
+        out[121] = h27;
+        out[132] = h30;
+        out[143] = h33;
+        out[154] = h35;
+        out[165] = h37;
+        out[176] = h38;
+        out[187] = h40;
+        out[198] = h43;
+        out[209] = h45;
+        out[220] = h47;
+        out[231] = h49;
+        out[242] = h51;
+        out[253] = h53;
+        out[264] = h56;
+        out[275] = h58;
+        out[286] = h60;
+        out[297] = h62;
+        out[308] = h63;
+        out[319] = h65;
+        out[330] = h68;
+        out[341] = h71;
+        out[352] = h73;
+        out[363] = h75;
+        out[374] = h76;
+        out[385] = h78;
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        out[0] = in[0] * (nrm * 0.2581988897471611);
+        out[1] = in[1] * (nrm * 0.5773502691896258);
+        out[2] = in[2] * (nrm * 0.5773502691896258);
+        out[3] = in[3] * (nrm * 0.5773502691896258);
+        out[4] = in[4] * (nrm * 0.5773502691896258);
+        out[5] = in[5] * (nrm * 1.0);
+        out[6] = in[6] * (nrm * 0.2581988897471611);
+        out[7] = in[7] * (nrm * 0.5773502691896258);
+        out[8] = in[8] * (nrm * 0.5773502691896258);
+        out[9] = in[9] * (nrm * 0.2581988897471611);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_ddfs[310] = {
-    11, 266, 65546, 521, 131081, 65801, 776, 66056, 131336, 196616, 1031, 1286,
-    66566, 1541, 132101, 66821, 1796, 67076, 132356, 197636, 262151, 262406, 327686, 262661,
-    393221, 327941, 262916, 328196, 393476, 458756, 2051, 2306, 67586, 2561, 133121, 67841,
-    2816, 68096, 133376, 198656, 263171, 263426, 328706, 263681, 394241, 328961, 263936, 329216,
-    394496, 459776, 524291, 524546, 589826, 524801, 655361, 590081, 525056, 590336, 655616, 720896,
-    15, 270, 65550, 525, 131085, 65805, 780, 66060, 131340, 196620, 1035, 1290,
-    66570, 1545, 132105, 66825, 1800, 67080, 132360, 197640, 262155, 262410, 327690, 262665,
-    393225, 327945, 262920, 328200, 393480, 458760, 2055, 2310, 67590, 2565, 133125, 67845,
-    2820, 68100, 133380, 198660, 524295, 524550, 589830, 524805, 655365, 590085, 525060, 590340,
-    655620, 720900, 263175, 263430, 328710, 263685, 394245, 328965, 263940, 329220, 394500, 459780,
-    3075, 3330, 68610, 3585, 134145, 68865, 3840, 69120, 134400, 199680, 264195, 264450,
-    329730, 264705, 395265, 329985, 264960, 330240, 395520, 460800, 525315, 525570, 590850, 525825,
-    656385, 591105, 526080, 591360, 656640, 721920, 786435, 786690, 851970, 786945, 917505, 852225,
-    787200, 852480, 917760, 983040, 19, 274, 65554, 529, 131089, 65809, 784, 66064,
-    131344, 196624, 1039, 1294, 66574, 1549, 132109, 66829, 1804, 67084, 132364, 197644,
-    262159, 262414, 327694, 262669, 393229, 327949, 262924, 328204, 393484, 458764, 2059, 2314,
-    67594, 2569, 133129, 67849, 2824, 68104, 133384, 198664, 263179, 263434, 328714, 263689,
-    394249, 328969, 263944, 329224, 394504, 459784, 524299, 524554, 589834, 524809, 655369, 590089,
-    525064, 590344, 655624, 720904, 3079, 3334, 68614, 3589, 134149, 68869, 3844, 69124,
-    134404, 199684, 264199, 264454, 329734, 264709, 395269, 329989, 264964, 330244, 395524, 460804,
-    525319, 525574, 590854, 525829, 656389, 591109, 526084, 591364, 656644, 721924, 786439, 786694,
-    851974, 786949, 917509, 852229, 787204, 852484, 917764, 983044, 4099, 4354, 69634, 4609,
-    135169, 69889, 4864, 70144, 135424, 200704, 265219, 265474, 330754, 265729, 396289, 331009,
-    265984, 331264, 396544, 461824, 526339, 526594, 591874, 526849, 657409, 592129, 527104, 592384,
-    657664, 722944, 787459, 787714, 852994, 787969, 918529, 853249, 788224, 853504, 918784, 984064,
-    1048579, 1048834, 1114114, 1049089, 1179649, 1114369, 1049344, 1114624, 1179904, 1245184,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_ddfs[37] = {
-    0, 3, 7, 11, 14, 18, 21, 24, 28, 32, 35, 39,
-    42, 45, 49, 53, 56, 60, 63, 66, 70, 74, 77, 81,
-    84, 87, 91, 95, 98, 102, 105, 108, 112, 116, 119, 123,
-    126,
-};
-__device__ const uint32_t kBraTerm_ddfs[126] = {
-    66560, 131334, 65552, 66816, 65799, 66054, 65553, 67072, 65800, 66310, 65554, 67328,
-    131591, 65555, 67584, 66056, 66311, 65556, 67840, 131848, 65557, 66561, 131335, 65553,
-    66817, 65801, 66055, 65555, 67073, 65803, 66311, 65556, 67329, 131593, 65558, 67585,
-    66059, 66313, 65559, 67841, 131851, 65560, 66562, 131336, 65554, 66818, 65803, 66056,
-    65556, 67074, 65802, 66312, 65557, 67330, 131595, 65559, 67586, 66058, 66315, 65560,
-    67842, 131850, 65561, 66563, 131337, 65555, 66819, 65804, 66057, 65558, 67075, 65805,
-    66313, 65559, 67331, 131596, 65562, 67587, 66061, 66316, 65563, 67843, 131853, 65564,
-    66564, 131339, 65556, 66820, 65805, 66059, 65559, 67076, 65806, 66315, 65560, 67332,
-    131597, 65563, 67588, 66062, 66317, 65564, 67844, 131854, 65565, 66565, 131338, 65557,
-    66821, 65806, 66058, 65560, 67077, 65807, 66314, 65561, 67333, 131598, 65564, 67589,
-    66063, 66318, 65565, 67845, 131855, 65566,
-};
-__device__ const uint16_t kKetOff_ddfs[11] = {
-    0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10,
-};
-__device__ const uint32_t kKetTerm_ddfs[10] = {
-    65536, 65537, 65538, 65539, 65540, 65541, 65542, 65543, 65544, 65545,
-};
 __device__ const double kNormAB_ddfs[36] = {
     0.3333333333333334, 0.5773502691896258, 0.5773502691896258, 0.3333333333333334,
     0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 1.0,
@@ -85,16 +194,12 @@ __device__ const double kNormAB_ddfs[36] = {
     1.0, 0.5773502691896258, 0.3333333333333334, 0.5773502691896258,
     0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 0.3333333333333334,
 };
-__device__ const double kNormCD_ddfs[10] = {
-    0.2581988897471611, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
-    0.5773502691896258, 1.0, 0.2581988897471611, 0.5773502691896258,
-    0.5773502691896258, 0.2581988897471611,
-};
 
+// column components cx | cy << 4 | cz << 8
+__device__ const uint16_t kCol_ddfs[10] = { 3, 18, 258, 33, 513, 273, 48, 288, 528, 768 };
 
 __device__ __forceinline__ RysClassTabs tabs_ddfs() {
-    return RysClassTabs{kBlk_ddfs, kBraOff_ddfs, kBraTerm_ddfs, kKetOff_ddfs, kKetTerm_ddfs,
-                        kNormAB_ddfs, kNormCD_ddfs, nullptr};
+    return RysClassTabs{kNormAB_ddfs, kCol_ddfs};
 }
 
 template <int MIXED>
@@ -107,8 +212,8 @@ static void rys_prepare_ddfs() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_ddfs<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 62080);
-        cudaFuncSetAttribute(rys_queue_ddfs<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 62080);
+        cudaFuncSetAttribute(rys_queue_ddfs<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 76032);
+        cudaFuncSetAttribute(rys_queue_ddfs<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 76032);
 
         done[dev] = true;
     }
@@ -120,16 +225,16 @@ void launch_rys_ddfs(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_ddfs();
     constexpr int ng = 128 / C_ddfs::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_ddfs<1><<<grid, 128, 62080, s>>>(Q, R);
-    else rys_queue_ddfs<0><<<grid, 128, 62080, s>>>(Q, R);
+    if (mixed) rys_queue_ddfs<1><<<grid, 128, 76032, s>>>(Q, R);
+    else rys_queue_ddfs<0><<<grid, 128, 76032, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_ddfs(int mixed) {
     rys_prepare_ddfs();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_ddfs<1>, 128, 62080);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_ddfs<0>, 128, 62080);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_ddfs<1>, 128, 76032);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_ddfs<0>, 128, 76032);
     return n;
 }
 

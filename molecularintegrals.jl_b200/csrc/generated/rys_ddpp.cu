@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (dd|pp).  Do not edit.
-// roots 4, block 31 x 9, outputs 36 x 9, group 64 threads,
-// 16 primitive quartets per batch, 1 slot(s), 5 accumulators per thread, 46720 B shared per block.
+// roots 4, block 31 x 9, outputs 36 x 9, group 32 threads, 3 ket pairs a round,
+// 2 primitive quartets per ket pair and batch, 62208 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,68 +11,186 @@ struct C_ddpp {
     static constexpr int NA = 31, NC = 9, NBLK = 279;
     static constexpr int NB = 6, ND = 3;
     static constexpr int NAB = 36, NCD = 9;
-    static constexpr int G = 64, NPB = 16, NSLOT = 1, ACC = 5;
-    static constexpr int S = 15;
-    static constexpr int SMEM_GROUP = 2920;
-    static constexpr bool COL = false;
+    static constexpr int G = 32, W = 3, H = 1, PB = 2;
+    static constexpr int S = 15, SI = 45, NCP = 9, NCDP = 9;
+    static constexpr int SMEM_GROUP = 1944;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
-    __device__ __forceinline__ static void col_update(const T *, const T *, const T *, A *) {}
+    __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
+        acc[0] = fma(x[2] * y[0], z[0], acc[0]);
+        acc[1] = fma(x[1] * y[1], z[0], acc[1]);
+        acc[2] = fma(x[1] * y[0], z[1], acc[2]);
+        acc[3] = fma(x[0] * y[2], z[0], acc[3]);
+        acc[4] = fma(x[0] * y[1], z[1], acc[4]);
+        acc[5] = fma(x[0] * y[0], z[2], acc[5]);
+        acc[6] = fma(x[3] * y[0], z[0], acc[6]);
+        acc[7] = fma(x[2] * y[1], z[0], acc[7]);
+        acc[8] = fma(x[2] * y[0], z[1], acc[8]);
+        acc[9] = fma(x[1] * y[2], z[0], acc[9]);
+        acc[10] = fma(x[1] * y[0], z[2], acc[10]);
+        acc[11] = fma(x[1] * y[1], z[1], acc[11]);
+        acc[12] = fma(x[0] * y[3], z[0], acc[12]);
+        acc[13] = fma(x[0] * y[2], z[1], acc[13]);
+        acc[14] = fma(x[0] * y[1], z[2], acc[14]);
+        acc[15] = fma(x[0] * y[0], z[3], acc[15]);
+        acc[16] = fma(x[4] * y[0], z[0], acc[16]);
+        acc[17] = fma(x[3] * y[1], z[0], acc[17]);
+        acc[18] = fma(x[3] * y[0], z[1], acc[18]);
+        acc[19] = fma(x[2] * y[2], z[0], acc[19]);
+        acc[20] = fma(x[2] * y[1], z[1], acc[20]);
+        acc[21] = fma(x[2] * y[0], z[2], acc[21]);
+        acc[22] = fma(x[1] * y[3], z[0], acc[22]);
+        acc[23] = fma(x[1] * y[2], z[1], acc[23]);
+        acc[24] = fma(x[1] * y[1], z[2], acc[24]);
+        acc[25] = fma(x[1] * y[0], z[3], acc[25]);
+        acc[26] = fma(x[0] * y[4], z[0], acc[26]);
+        acc[27] = fma(x[0] * y[3], z[1], acc[27]);
+        acc[28] = fma(x[0] * y[2], z[2], acc[28]);
+        acc[29] = fma(x[0] * y[1], z[3], acc[29]);
+        acc[30] = fma(x[0] * y[0], z[4], acc[30]);
+    }
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[6], in[16]);
+        const double h1 = fma(x, in[0], in[6]);
+        const double h2 = fma(x, h1, h0);
+        const double h3 = fma(y, in[6], in[17]);
+        const double h4 = fma(y, in[0], in[7]);
+        const double h5 = fma(x, h4, h3);
+        const double h6 = fma(z, in[6], in[18]);
+        const double h7 = fma(z, in[0], in[8]);
+        const double h8 = fma(x, h7, h6);
+        const double h9 = fma(y, in[7], in[19]);
+        const double h10 = fma(y, h4, h9);
+        const double h11 = fma(z, in[7], in[20]);
+        const double h12 = fma(y, h7, h11);
+        const double h13 = fma(z, in[8], in[21]);
+        const double h14 = fma(z, h7, h13);
+        const double h15 = fma(x, in[7], in[17]);
+        const double h16 = fma(x, in[1], in[7]);
+        const double h17 = fma(x, h16, h15);
+        const double h18 = fma(y, in[1], in[9]);
+        const double h19 = fma(x, h18, h9);
+        const double h20 = fma(z, in[1], in[11]);
+        const double h21 = fma(x, h20, h11);
+        const double h22 = fma(y, in[9], in[22]);
+        const double h23 = fma(y, h18, h22);
+        const double h24 = fma(z, in[9], in[23]);
+        const double h25 = fma(y, h20, h24);
+        const double h26 = fma(z, in[11], in[24]);
+        const double h27 = fma(z, h20, h26);
+        const double h28 = fma(x, in[8], in[18]);
+        const double h29 = fma(x, in[2], in[8]);
+        const double h30 = fma(x, h29, h28);
+        const double h31 = fma(y, in[8], in[20]);
+        const double h32 = fma(y, in[2], in[11]);
+        const double h33 = fma(x, h32, h31);
+        const double h34 = fma(z, in[2], in[10]);
+        const double h35 = fma(x, h34, h13);
+        const double h36 = fma(y, in[11], in[23]);
+        const double h37 = fma(y, h32, h36);
+        const double h38 = fma(y, h34, h26);
+        const double h39 = fma(z, in[10], in[25]);
+        const double h40 = fma(z, h34, h39);
+        const double h41 = fma(x, in[9], in[19]);
+        const double h42 = fma(x, in[3], in[9]);
+        const double h43 = fma(x, h42, h41);
+        const double h44 = fma(y, in[3], in[12]);
+        const double h45 = fma(x, h44, h22);
+        const double h46 = fma(z, in[3], in[13]);
+        const double h47 = fma(x, h46, h24);
+        const double h48 = fma(y, in[12], in[26]);
+        const double h49 = fma(y, h44, h48);
+        const double h50 = fma(z, in[12], in[27]);
+        const double h51 = fma(y, h46, h50);
+        const double h52 = fma(z, in[13], in[28]);
+        const double h53 = fma(z, h46, h52);
+        const double h54 = fma(x, in[11], in[20]);
+        const double h55 = fma(x, in[4], in[11]);
+        const double h56 = fma(x, h55, h54);
+        const double h57 = fma(y, in[4], in[13]);
+        const double h58 = fma(x, h57, h36);
+        const double h59 = fma(z, in[4], in[14]);
+        const double h60 = fma(x, h59, h26);
+        const double h61 = fma(y, in[13], in[27]);
+        const double h62 = fma(y, h57, h61);
+        const double h63 = fma(y, h59, h52);
+        const double h64 = fma(z, in[14], in[29]);
+        const double h65 = fma(z, h59, h64);
+        const double h66 = fma(x, in[10], in[21]);
+        const double h67 = fma(x, in[5], in[10]);
+        const double h68 = fma(x, h67, h66);
+        const double h69 = fma(y, in[10], in[24]);
+        const double h70 = fma(y, in[5], in[14]);
+        const double h71 = fma(x, h70, h69);
+        const double h72 = fma(z, in[5], in[15]);
+        const double h73 = fma(x, h72, h39);
+        const double h74 = fma(y, in[14], in[28]);
+        const double h75 = fma(y, h70, h74);
+        const double h76 = fma(y, h72, h64);
+        const double h77 = fma(z, in[15], in[30]);
+        const double h78 = fma(z, h72, h77);
+        out[0] = h2;
+        out[9] = h5;
+        out[18] = h8;
+        out[27] = h10;
+        out[36] = h12;
+        out[45] = h14;
+        out[54] = h17;
+        out[63] = h19;
+        out[72] = h21;
+        out[81] = h23;
+        out[90] = h25;
+        out[99] = h27;
+        out[108] = h30;
+        out[117] = h33;
+        out[126] = h35;
+        out[135] = h37;
+        out[144] = h38;
+        out[153] = h40;
+        out[162] = h43;
+        out[171] = h45;
+        out[180] = h47;
+        out[189] = h49;
+        out[198] = h51;
+        out[207] = h53;
+        out[216] = h56;
+        out[225] = h58;
+        out[234] = h60;
+        out[243] = h62;
+        out[252] = h63;
+        out[261] = h65;
+        out[270] = h68;
+        out[279] = h71;
+        out[288] = h73;
+        out[297] = h75;
+        out[306] = h76;
+        out[315] = h78;
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[0], in[3]);
+        const double h1 = fma(y, in[0], in[4]);
+        const double h2 = fma(z, in[0], in[5]);
+        const double h3 = fma(x, in[1], in[4]);
+        const double h4 = fma(y, in[1], in[6]);
+        const double h5 = fma(z, in[1], in[7]);
+        const double h6 = fma(x, in[2], in[5]);
+        const double h7 = fma(y, in[2], in[7]);
+        const double h8 = fma(z, in[2], in[8]);
+        out[0] = h0 * (nrm * 1.0);
+        out[1] = h1 * (nrm * 1.0);
+        out[2] = h2 * (nrm * 1.0);
+        out[3] = h3 * (nrm * 1.0);
+        out[4] = h4 * (nrm * 1.0);
+        out[5] = h5 * (nrm * 1.0);
+        out[6] = h6 * (nrm * 1.0);
+        out[7] = h7 * (nrm * 1.0);
+        out[8] = h8 * (nrm * 1.0);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_ddpp[279] = {
-    7, 262, 65542, 8, 263, 65543, 518, 65798, 131078, 772, 1027, 66307,
-    773, 1028, 66308, 1283, 66563, 131843, 196612, 196867, 262147, 196613, 196868, 262148,
-    197123, 262403, 327683, 1537, 1792, 67072, 1538, 1793, 67073, 2048, 67328, 132608,
-    197377, 197632, 262912, 197378, 197633, 262913, 197888, 263168, 328448, 393217, 393472, 458752,
-    393218, 393473, 458753, 393728, 459008, 524288, 10, 265, 65545, 11, 266, 65546,
-    521, 65801, 131081, 775, 1030, 66310, 776, 1031, 66311, 1286, 66566, 131846,
-    196615, 196870, 262150, 196616, 196871, 262151, 197126, 262406, 327686, 1540, 1795, 67075,
-    1541, 1796, 67076, 2051, 67331, 132611, 393220, 393475, 458755, 393221, 393476, 458756,
-    393731, 459011, 524291, 197380, 197635, 262915, 197381, 197636, 262916, 197891, 263171, 328451,
-    2305, 2560, 67840, 2306, 2561, 67841, 2816, 68096, 133376, 198145, 198400, 263680,
-    198146, 198401, 263681, 198656, 263936, 329216, 393985, 394240, 459520, 393986, 394241, 459521,
-    394496, 459776, 525056, 589825, 590080, 655360, 589826, 590081, 655361, 590336, 655616, 720896,
-    13, 268, 65548, 14, 269, 65549, 524, 65804, 131084, 778, 1033, 66313,
-    779, 1034, 66314, 1289, 66569, 131849, 196618, 196873, 262153, 196619, 196874, 262154,
-    197129, 262409, 327689, 1543, 1798, 67078, 1544, 1799, 67079, 2054, 67334, 132614,
-    197383, 197638, 262918, 197384, 197639, 262919, 197894, 263174, 328454, 393223, 393478, 458758,
-    393224, 393479, 458759, 393734, 459014, 524294, 2308, 2563, 67843, 2309, 2564, 67844,
-    2819, 68099, 133379, 198148, 198403, 263683, 198149, 198404, 263684, 198659, 263939, 329219,
-    393988, 394243, 459523, 393989, 394244, 459524, 394499, 459779, 525059, 589828, 590083, 655363,
-    589829, 590084, 655364, 590339, 655619, 720899, 3073, 3328, 68608, 3074, 3329, 68609,
-    3584, 68864, 134144, 198913, 199168, 264448, 198914, 199169, 264449, 199424, 264704, 329984,
-    394753, 395008, 460288, 394754, 395009, 460289, 395264, 460544, 525824, 590593, 590848, 656128,
-    590594, 590849, 656129, 591104, 656384, 721664, 786433, 786688, 851968, 786434, 786689, 851969,
-    786944, 852224, 917504,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_ddpp[37] = {
-    0, 3, 7, 11, 14, 18, 21, 24, 28, 32, 35, 39,
-    42, 45, 49, 53, 56, 60, 63, 66, 70, 74, 77, 81,
-    84, 87, 91, 95, 98, 102, 105, 108, 112, 116, 119, 123,
-    126,
-};
-__device__ const uint32_t kBraTerm_ddpp[126] = {
-    66560, 131334, 65552, 66816, 65799, 66054, 65553, 67072, 65800, 66310, 65554, 67328,
-    131591, 65555, 67584, 66056, 66311, 65556, 67840, 131848, 65557, 66561, 131335, 65553,
-    66817, 65801, 66055, 65555, 67073, 65803, 66311, 65556, 67329, 131593, 65558, 67585,
-    66059, 66313, 65559, 67841, 131851, 65560, 66562, 131336, 65554, 66818, 65803, 66056,
-    65556, 67074, 65802, 66312, 65557, 67330, 131595, 65559, 67586, 66058, 66315, 65560,
-    67842, 131850, 65561, 66563, 131337, 65555, 66819, 65804, 66057, 65558, 67075, 65805,
-    66313, 65559, 67331, 131596, 65562, 67587, 66061, 66316, 65563, 67843, 131853, 65564,
-    66564, 131339, 65556, 66820, 65805, 66059, 65559, 67076, 65806, 66315, 65560, 67332,
-    131597, 65563, 67588, 66062, 66317, 65564, 67844, 131854, 65565, 66565, 131338, 65557,
-    66821, 65806, 66058, 65560, 67077, 65807, 66314, 65561, 67333, 131598, 65564, 67589,
-    66063, 66318, 65565, 67845, 131855, 65566,
-};
-__device__ const uint16_t kKetOff_ddpp[10] = {
-    0, 2, 4, 6, 8, 10, 12, 14, 16, 18,
-};
-__device__ const uint32_t kKetTerm_ddpp[18] = {
-    65792, 65539, 66048, 65540, 66304, 65541, 65793, 65540, 66049, 65542, 66305, 65543,
-    65794, 65541, 66050, 65543, 66306, 65544,
-};
 __device__ const double kNormAB_ddpp[36] = {
     0.3333333333333334, 0.5773502691896258, 0.5773502691896258, 0.3333333333333334,
     0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 1.0,
@@ -84,16 +202,12 @@ __device__ const double kNormAB_ddpp[36] = {
     1.0, 0.5773502691896258, 0.3333333333333334, 0.5773502691896258,
     0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 0.3333333333333334,
 };
-__device__ const double kNormCD_ddpp[9] = {
-    1.0, 1.0, 1.0, 1.0,
-    1.0, 1.0, 1.0, 1.0,
-    1.0,
-};
 
+// column components cx | cy << 4 | cz << 8
+__device__ const uint16_t kCol_ddpp[9] = { 1, 16, 256, 2, 17, 257, 32, 272, 512 };
 
 __device__ __forceinline__ RysClassTabs tabs_ddpp() {
-    return RysClassTabs{kBlk_ddpp, kBraOff_ddpp, kBraTerm_ddpp, kKetOff_ddpp, kKetTerm_ddpp,
-                        kNormAB_ddpp, kNormCD_ddpp, nullptr};
+    return RysClassTabs{kNormAB_ddpp, kCol_ddpp};
 }
 
 template <int MIXED>
@@ -106,8 +220,8 @@ static void rys_prepare_ddpp() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_ddpp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 46720);
-        cudaFuncSetAttribute(rys_queue_ddpp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 46720);
+        cudaFuncSetAttribute(rys_queue_ddpp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 62208);
+        cudaFuncSetAttribute(rys_queue_ddpp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 62208);
 
         done[dev] = true;
     }
@@ -119,16 +233,16 @@ void launch_rys_ddpp(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_ddpp();
     constexpr int ng = 128 / C_ddpp::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_ddpp<1><<<grid, 128, 46720, s>>>(Q, R);
-    else rys_queue_ddpp<0><<<grid, 128, 46720, s>>>(Q, R);
+    if (mixed) rys_queue_ddpp<1><<<grid, 128, 62208, s>>>(Q, R);
+    else rys_queue_ddpp<0><<<grid, 128, 62208, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_ddpp(int mixed) {
     rys_prepare_ddpp();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_ddpp<1>, 128, 46720);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_ddpp<0>, 128, 46720);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_ddpp<1>, 128, 62208);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_ddpp<0>, 128, 62208);
     return n;
 }
 

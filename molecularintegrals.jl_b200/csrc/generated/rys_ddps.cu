@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (dd|ps).  Do not edit.
-// roots 3, block 31 x 3, outputs 36 x 3, group 32 threads,
-// 10 primitive quartets per batch, 1 slot(s), 3 accumulators per thread, 30080 B shared per block.
+// roots 3, block 31 x 3, outputs 36 x 3, group 32 threads, 5 ket pairs a round,
+// 2 primitive quartets per ket pair and batch, 34560 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,51 +11,171 @@ struct C_ddps {
     static constexpr int NA = 31, NC = 3, NBLK = 93;
     static constexpr int NB = 6, ND = 1;
     static constexpr int NAB = 36, NCD = 3;
-    static constexpr int G = 32, NPB = 10, NSLOT = 1, ACC = 3;
-    static constexpr int S = 10;
-    static constexpr int SMEM_GROUP = 940;
-    static constexpr bool COL = false;
+    static constexpr int G = 32, W = 5, H = 2, PB = 2;
+    static constexpr int S = 10, SI = 31, NCP = 3, NCDP = 3;
+    static constexpr int SMEM_GROUP = 1080;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
-    __device__ __forceinline__ static void col_update(const T *, const T *, const T *, A *) {}
+    __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
+        acc[0] = fma(x[2] * y[0], z[0], acc[0]);
+        acc[1] = fma(x[1] * y[1], z[0], acc[1]);
+        acc[2] = fma(x[1] * y[0], z[1], acc[2]);
+        acc[3] = fma(x[0] * y[2], z[0], acc[3]);
+        acc[4] = fma(x[0] * y[1], z[1], acc[4]);
+        acc[5] = fma(x[0] * y[0], z[2], acc[5]);
+        acc[6] = fma(x[3] * y[0], z[0], acc[6]);
+        acc[7] = fma(x[2] * y[1], z[0], acc[7]);
+        acc[8] = fma(x[2] * y[0], z[1], acc[8]);
+        acc[9] = fma(x[1] * y[2], z[0], acc[9]);
+        acc[10] = fma(x[1] * y[0], z[2], acc[10]);
+        acc[11] = fma(x[1] * y[1], z[1], acc[11]);
+        acc[12] = fma(x[0] * y[3], z[0], acc[12]);
+        acc[13] = fma(x[0] * y[2], z[1], acc[13]);
+        acc[14] = fma(x[0] * y[1], z[2], acc[14]);
+        acc[15] = fma(x[0] * y[0], z[3], acc[15]);
+        acc[16] = fma(x[4] * y[0], z[0], acc[16]);
+        acc[17] = fma(x[3] * y[1], z[0], acc[17]);
+        acc[18] = fma(x[3] * y[0], z[1], acc[18]);
+        acc[19] = fma(x[2] * y[2], z[0], acc[19]);
+        acc[20] = fma(x[2] * y[1], z[1], acc[20]);
+        acc[21] = fma(x[2] * y[0], z[2], acc[21]);
+        acc[22] = fma(x[1] * y[3], z[0], acc[22]);
+        acc[23] = fma(x[1] * y[2], z[1], acc[23]);
+        acc[24] = fma(x[1] * y[1], z[2], acc[24]);
+        acc[25] = fma(x[1] * y[0], z[3], acc[25]);
+        acc[26] = fma(x[0] * y[4], z[0], acc[26]);
+        acc[27] = fma(x[0] * y[3], z[1], acc[27]);
+        acc[28] = fma(x[0] * y[2], z[2], acc[28]);
+        acc[29] = fma(x[0] * y[1], z[3], acc[29]);
+        acc[30] = fma(x[0] * y[0], z[4], acc[30]);
+    }
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[6], in[16]);
+        const double h1 = fma(x, in[0], in[6]);
+        const double h2 = fma(x, h1, h0);
+        const double h3 = fma(y, in[6], in[17]);
+        const double h4 = fma(y, in[0], in[7]);
+        const double h5 = fma(x, h4, h3);
+        const double h6 = fma(z, in[6], in[18]);
+        const double h7 = fma(z, in[0], in[8]);
+        const double h8 = fma(x, h7, h6);
+        const double h9 = fma(y, in[7], in[19]);
+        const double h10 = fma(y, h4, h9);
+        const double h11 = fma(z, in[7], in[20]);
+        const double h12 = fma(y, h7, h11);
+        const double h13 = fma(z, in[8], in[21]);
+        const double h14 = fma(z, h7, h13);
+        const double h15 = fma(x, in[7], in[17]);
+        const double h16 = fma(x, in[1], in[7]);
+        const double h17 = fma(x, h16, h15);
+        const double h18 = fma(y, in[1], in[9]);
+        const double h19 = fma(x, h18, h9);
+        const double h20 = fma(z, in[1], in[11]);
+        const double h21 = fma(x, h20, h11);
+        const double h22 = fma(y, in[9], in[22]);
+        const double h23 = fma(y, h18, h22);
+        const double h24 = fma(z, in[9], in[23]);
+        const double h25 = fma(y, h20, h24);
+        const double h26 = fma(z, in[11], in[24]);
+        const double h27 = fma(z, h20, h26);
+        const double h28 = fma(x, in[8], in[18]);
+        const double h29 = fma(x, in[2], in[8]);
+        const double h30 = fma(x, h29, h28);
+        const double h31 = fma(y, in[8], in[20]);
+        const double h32 = fma(y, in[2], in[11]);
+        const double h33 = fma(x, h32, h31);
+        const double h34 = fma(z, in[2], in[10]);
+        const double h35 = fma(x, h34, h13);
+        const double h36 = fma(y, in[11], in[23]);
+        const double h37 = fma(y, h32, h36);
+        const double h38 = fma(y, h34, h26);
+        const double h39 = fma(z, in[10], in[25]);
+        const double h40 = fma(z, h34, h39);
+        const double h41 = fma(x, in[9], in[19]);
+        const double h42 = fma(x, in[3], in[9]);
+        const double h43 = fma(x, h42, h41);
+        const double h44 = fma(y, in[3], in[12]);
+        const double h45 = fma(x, h44, h22);
+        const double h46 = fma(z, in[3], in[13]);
+        const double h47 = fma(x, h46, h24);
+        const double h48 = fma(y, in[12], in[26]);
+        const double h49 = fma(y, h44, h48);
+        const double h50 = fma(z, in[12], in[27]);
+        const double h51 = fma(y, h46, h50);
+        const double h52 = fma(z, in[13], in[28]);
+        const double h53 = fma(z, h46, h52);
+        const double h54 = fma(x, in[11], in[20]);
+        const double h55 = fma(x, in[4], in[11]);
+        const double h56 = fma(x, h55, h54);
+        const double h57 = fma(y, in[4], in[13]);
+        const double h58 = fma(x, h57, h36);
+        const double h59 = fma(z, in[4], in[14]);
+        const double h60 = fma(x, h59, h26);
+        const double h61 = fma(y, in[13], in[27]);
+        const double h62 = fma(y, h57, h61);
+        const double h63 = fma(y, h59, h52);
+        const double h64 = fma(z, in[14], in[29]);
+        const double h65 = fma(z, h59, h64);
+        const double h66 = fma(x, in[10], in[21]);
+        const double h67 = fma(x, in[5], in[10]);
+        const double h68 = fma(x, h67, h66);
+        const double h69 = fma(y, in[10], in[24]);
+        const double h70 = fma(y, in[5], in[14]);
+        const double h71 = fma(x, h70, h69);
+        const double h72 = fma(z, in[5], in[15]);
+        const double h73 = fma(x, h72, h39);
+        const double h74 = fma(y, in[14], in[28]);
+        const double h75 = fma(y, h70, h74);
+        const double h76 = fma(y, h72, h64);
+        const double h77 = fma(z, in[15], in[30]);
+        const double h78 = fma(z, h72, h77);
+        out[0] = h2;
+        out[3] = h5;
+        out[6] = h8;
+        out[9] = h10;
+        out[12] = h12;
+        out[15] = h14;
+        out[18] = h17;
+        out[21] = h19;
+        out[24] = h21;
+        out[27] = h23;
+        out[30] = h25;
+        out[33] = h27;
+        out[36] = h30;
+        out[39] = h33;
+        out[42] = h35;
+        out[45] = h37;
+        out[48] = h38;
+        out[51] = h40;
+        out[54] = h43;
+        out[57] = h45;
+        out[60] = h47;
+        out[63] = h49;
+        out[66] = h51;
+        out[69] = h53;
+        out[72] = h56;
+        out[75] = h58;
+        out[78] = h60;
+        out[81] = h62;
+        out[84] = h63;
+        out[87] = h65;
+        out[90] = h68;
+        out[93] = h71;
+        out[96] = h73;
+        out[99] = h75;
+        out[102] = h76;
+        out[105] = h78;
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        out[0] = in[0] * (nrm * 1.0);
+        out[1] = in[1] * (nrm * 1.0);
+        out[2] = in[2] * (nrm * 1.0);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_ddps[93] = {
-    5, 260, 65540, 515, 770, 66050, 131075, 131330, 196610, 1025, 1280, 66560,
-    131585, 131840, 197120, 262145, 262400, 327680, 7, 262, 65542, 517, 772, 66052,
-    131077, 131332, 196612, 1027, 1282, 66562, 262147, 262402, 327682, 131587, 131842, 197122,
-    1537, 1792, 67072, 132097, 132352, 197632, 262657, 262912, 328192, 393217, 393472, 458752,
-    9, 264, 65544, 519, 774, 66054, 131079, 131334, 196614, 1029, 1284, 66564,
-    131589, 131844, 197124, 262149, 262404, 327684, 1539, 1794, 67074, 132099, 132354, 197634,
-    262659, 262914, 328194, 393219, 393474, 458754, 2049, 2304, 67584, 132609, 132864, 198144,
-    263169, 263424, 328704, 393729, 393984, 459264, 524289, 524544, 589824,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_ddps[37] = {
-    0, 3, 7, 11, 14, 18, 21, 24, 28, 32, 35, 39,
-    42, 45, 49, 53, 56, 60, 63, 66, 70, 74, 77, 81,
-    84, 87, 91, 95, 98, 102, 105, 108, 112, 116, 119, 123,
-    126,
-};
-__device__ const uint32_t kBraTerm_ddps[126] = {
-    66560, 131334, 65552, 66816, 65799, 66054, 65553, 67072, 65800, 66310, 65554, 67328,
-    131591, 65555, 67584, 66056, 66311, 65556, 67840, 131848, 65557, 66561, 131335, 65553,
-    66817, 65801, 66055, 65555, 67073, 65803, 66311, 65556, 67329, 131593, 65558, 67585,
-    66059, 66313, 65559, 67841, 131851, 65560, 66562, 131336, 65554, 66818, 65803, 66056,
-    65556, 67074, 65802, 66312, 65557, 67330, 131595, 65559, 67586, 66058, 66315, 65560,
-    67842, 131850, 65561, 66563, 131337, 65555, 66819, 65804, 66057, 65558, 67075, 65805,
-    66313, 65559, 67331, 131596, 65562, 67587, 66061, 66316, 65563, 67843, 131853, 65564,
-    66564, 131339, 65556, 66820, 65805, 66059, 65559, 67076, 65806, 66315, 65560, 67332,
-    131597, 65563, 67588, 66062, 66317, 65564, 67844, 131854, 65565, 66565, 131338, 65557,
-    66821, 65806, 66058, 65560, 67077, 65807, 66314, 65561, 67333, 131598, 65564, 67589,
-    66063, 66318, 65565, 67845, 131855, 65566,
-};
-__device__ const uint16_t kKetOff_ddps[4] = {
-    0, 1, 2, 3,
-};
-__device__ const uint32_t kKetTerm_ddps[3] = {
-    65536, 65537, 65538,
-};
 __device__ const double kNormAB_ddps[36] = {
     0.3333333333333334, 0.5773502691896258, 0.5773502691896258, 0.3333333333333334,
     0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 1.0,
@@ -67,14 +187,12 @@ __device__ const double kNormAB_ddps[36] = {
     1.0, 0.5773502691896258, 0.3333333333333334, 0.5773502691896258,
     0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 0.3333333333333334,
 };
-__device__ const double kNormCD_ddps[3] = {
-    1.0, 1.0, 1.0,
-};
 
+// column components cx | cy << 4 | cz << 8
+__device__ const uint16_t kCol_ddps[3] = { 1, 16, 256 };
 
 __device__ __forceinline__ RysClassTabs tabs_ddps() {
-    return RysClassTabs{kBlk_ddps, kBraOff_ddps, kBraTerm_ddps, kKetOff_ddps, kKetTerm_ddps,
-                        kNormAB_ddps, kNormCD_ddps, nullptr};
+    return RysClassTabs{kNormAB_ddps, kCol_ddps};
 }
 
 template <int MIXED>
@@ -87,8 +205,8 @@ static void rys_prepare_ddps() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_ddps<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 30080);
-        cudaFuncSetAttribute(rys_queue_ddps<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 30080);
+        cudaFuncSetAttribute(rys_queue_ddps<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 34560);
+        cudaFuncSetAttribute(rys_queue_ddps<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 34560);
 
         done[dev] = true;
     }
@@ -100,16 +218,16 @@ void launch_rys_ddps(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_ddps();
     constexpr int ng = 128 / C_ddps::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_ddps<1><<<grid, 128, 30080, s>>>(Q, R);
-    else rys_queue_ddps<0><<<grid, 128, 30080, s>>>(Q, R);
+    if (mixed) rys_queue_ddps<1><<<grid, 128, 34560, s>>>(Q, R);
+    else rys_queue_ddps<0><<<grid, 128, 34560, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_ddps(int mixed) {
     rys_prepare_ddps();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_ddps<1>, 128, 30080);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_ddps<0>, 128, 30080);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_ddps<1>, 128, 34560);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_ddps<0>, 128, 34560);
     return n;
 }
 

@@ -1,110 +1,440 @@
 // Generated by gen_rys.py -- Rys class (dd|ss).  Do not edit.
-// roots 3, block 31 x 1, outputs 36 x 1, group 32 threads,
-// 10 primitive quartets per batch, 1 slot(s), 1 accumulators per thread, 15680 B shared per block.
+// roots 3, contracted block: 31, outputs: 36: a lane-split kernel, the lanes' primitive quartets by
+// Rys quadrature with the 2-D tables in registers.
 #include "../rys_common.cuh"
 
 namespace molints {
 
-struct C_ddss {
-    static constexpr int LA = 2, LB = 2, LC = 0, LD = 0;
-    static constexpr int E = 4, F = 0, NR = 3;
-    static constexpr int NA = 31, NC = 1, NBLK = 31;
-    static constexpr int NB = 6, ND = 1;
-    static constexpr int NAB = 36, NCD = 1;
-    static constexpr int G = 32, NPB = 10, NSLOT = 1, ACC = 1;
-    static constexpr int S = 5;
-    static constexpr int SMEM_GROUP = 490;
-    static constexpr bool COL = false;
-    template <typename T, typename A>
-    __device__ __forceinline__ static void col_update(const T *, const T *, const T *, A *) {}
-};
-
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_ddss[31] = {
-    2, 257, 65537, 512, 65792, 131072, 3, 258, 65538, 513, 131073, 65793,
-    768, 66048, 131328, 196608, 4, 259, 65539, 514, 65794, 131074, 769, 66049,
-    131329, 196609, 1024, 66304, 131584, 196864, 262144,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_ddss[37] = {
-    0, 3, 7, 11, 14, 18, 21, 24, 28, 32, 35, 39,
-    42, 45, 49, 53, 56, 60, 63, 66, 70, 74, 77, 81,
-    84, 87, 91, 95, 98, 102, 105, 108, 112, 116, 119, 123,
-    126,
-};
-__device__ const uint32_t kBraTerm_ddss[126] = {
-    66560, 131334, 65552, 66816, 65799, 66054, 65553, 67072, 65800, 66310, 65554, 67328,
-    131591, 65555, 67584, 66056, 66311, 65556, 67840, 131848, 65557, 66561, 131335, 65553,
-    66817, 65801, 66055, 65555, 67073, 65803, 66311, 65556, 67329, 131593, 65558, 67585,
-    66059, 66313, 65559, 67841, 131851, 65560, 66562, 131336, 65554, 66818, 65803, 66056,
-    65556, 67074, 65802, 66312, 65557, 67330, 131595, 65559, 67586, 66058, 66315, 65560,
-    67842, 131850, 65561, 66563, 131337, 65555, 66819, 65804, 66057, 65558, 67075, 65805,
-    66313, 65559, 67331, 131596, 65562, 67587, 66061, 66316, 65563, 67843, 131853, 65564,
-    66564, 131339, 65556, 66820, 65805, 66059, 65559, 67076, 65806, 66315, 65560, 67332,
-    131597, 65563, 67588, 66062, 66317, 65564, 67844, 131854, 65565, 66565, 131338, 65557,
-    66821, 65806, 66058, 65560, 67077, 65807, 66314, 65561, 67333, 131598, 65564, 67589,
-    66063, 66318, 65565, 67845, 131855, 65566,
-};
-__device__ const uint16_t kKetOff_ddss[2] = {
-    0, 1,
-};
-__device__ const uint32_t kKetTerm_ddss[1] = {
-    65536,
-};
-__device__ const double kNormAB_ddss[36] = {
-    0.3333333333333334, 0.5773502691896258, 0.5773502691896258, 0.3333333333333334,
-    0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 1.0,
-    1.0, 0.5773502691896258, 1.0, 0.5773502691896258,
-    0.5773502691896258, 1.0, 1.0, 0.5773502691896258,
-    1.0, 0.5773502691896258, 0.3333333333333334, 0.5773502691896258,
-    0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 0.3333333333333334,
-    0.5773502691896258, 1.0, 1.0, 0.5773502691896258,
-    1.0, 0.5773502691896258, 0.3333333333333334, 0.5773502691896258,
-    0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 0.3333333333333334,
-};
-__device__ const double kNormCD_ddss[1] = {
-    1.0,
-};
-
-
-__device__ __forceinline__ RysClassTabs tabs_ddss() {
-    return RysClassTabs{kBlk_ddss, kBraOff_ddss, kBraTerm_ddss, kKetOff_ddss, kKetTerm_ddss,
-                        kNormAB_ddss, kNormCD_ddss, nullptr};
-}
-
-template <int MIXED>
-__global__ void __launch_bounds__(128) rys_queue_ddss(const EriQueue Q, const RysTab R) {
-    rys_queue_body<C_ddss, MIXED>(Q, R, tabs_ddss());
-}
-
-static void rys_prepare_ddss() {
-    static bool done[64] = {false};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_ddss<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 15680);
-
-
-        done[dev] = true;
+// The contracted [e0|f0] block of bra pair p and ket pair q into acc[31] by the 3-point Rys
+// rule, summed over the bra primitive pairs i0, i0 + istep, ... < i1 and the ket primitive pairs
+// j0, j0 + jstep, ... < j1; loop order and splits as in the HGP kernel of the class.
+__device__ __forceinline__ void vrr_ddss_rys(const PairTab &P, const RysTab &R, int p, int q, int i0, int i1,
+                                          int istep, int j0, int j1, int jstep, double *__restrict__ acc) {
+    const int4 ib_ = __ldg(&P.info[p]);
+    const int4 ik_ = __ldg(&P.info[q]);
+#pragma unroll
+    for (int x = 0; x < 31; ++x) acc[x] = 0.0;
+    for (int j = j0; j < j1; j += jstep) {
+        const PrimPair ket = load_pp(P.pp, ik_.x + j);
+        for (int i = i0; i < i1; i += istep) {
+            const PrimPair bra = load_pp(P.pp, ib_.x + i);
+            const double r = rsqrt(bra.zeta + ket.zeta);
+            const double r2 = r * r;
+            const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
+            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double pref = bra.kab * ket.kab * r;
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+#pragma unroll 1
+            for (int k = 0; k < 3; ++k) {
+                double u, w;
+                rys_root<3>(R, T, k, u, w);
+                const double b10 = bra.oo2z * fma(-ez, u, 1.0), b01 = ket.oo2z * fma(-zz, u, 1.0), b00 = 0.5 * r2 * u;
+                (void)b10; (void)b01; (void)b00;
+                const double Cx = fma(-ez * PQx, u, bra.pax), Dx = fma(zz * PQx, u, ket.pax);
+                (void)Cx; (void)Dx;
+                const double Cy = fma(-ez * PQy, u, bra.pay), Dy = fma(zz * PQy, u, ket.pay);
+                (void)Cy; (void)Dy;
+                const double Cz = fma(-ez * PQz, u, bra.paz), Dz = fma(zz * PQz, u, ket.paz);
+                (void)Cz; (void)Dz;
+                const double x0_0 = pref * w;
+                const double x1_0 = Cx * x0_0;
+                const double x2_0 = Cx * x1_0 + 1.0 * b10 * x0_0;
+                const double x3_0 = Cx * x2_0 + 2.0 * b10 * x1_0;
+                const double x4_0 = Cx * x3_0 + 3.0 * b10 * x2_0;
+                const double y0_0 = 1.0;
+                const double y1_0 = Cy * y0_0;
+                const double y2_0 = Cy * y1_0 + 1.0 * b10 * y0_0;
+                const double y3_0 = Cy * y2_0 + 2.0 * b10 * y1_0;
+                const double y4_0 = Cy * y3_0 + 3.0 * b10 * y2_0;
+                const double z0_0 = 1.0;
+                const double z1_0 = Cz * z0_0;
+                const double z2_0 = Cz * z1_0 + 1.0 * b10 * z0_0;
+                const double z3_0 = Cz * z2_0 + 2.0 * b10 * z1_0;
+                const double z4_0 = Cz * z3_0 + 3.0 * b10 * z2_0;
+                acc[0] = fma(x2_0 * y0_0, z0_0, acc[0]);
+                acc[1] = fma(x1_0 * y1_0, z0_0, acc[1]);
+                acc[2] = fma(x1_0 * y0_0, z1_0, acc[2]);
+                acc[3] = fma(x0_0 * y2_0, z0_0, acc[3]);
+                acc[4] = fma(x0_0 * y1_0, z1_0, acc[4]);
+                acc[5] = fma(x0_0 * y0_0, z2_0, acc[5]);
+                acc[6] = fma(x3_0 * y0_0, z0_0, acc[6]);
+                acc[7] = fma(x2_0 * y1_0, z0_0, acc[7]);
+                acc[8] = fma(x2_0 * y0_0, z1_0, acc[8]);
+                acc[9] = fma(x1_0 * y2_0, z0_0, acc[9]);
+                acc[10] = fma(x1_0 * y0_0, z2_0, acc[10]);
+                acc[11] = fma(x1_0 * y1_0, z1_0, acc[11]);
+                acc[12] = fma(x0_0 * y3_0, z0_0, acc[12]);
+                acc[13] = fma(x0_0 * y2_0, z1_0, acc[13]);
+                acc[14] = fma(x0_0 * y1_0, z2_0, acc[14]);
+                acc[15] = fma(x0_0 * y0_0, z3_0, acc[15]);
+                acc[16] = fma(x4_0 * y0_0, z0_0, acc[16]);
+                acc[17] = fma(x3_0 * y1_0, z0_0, acc[17]);
+                acc[18] = fma(x3_0 * y0_0, z1_0, acc[18]);
+                acc[19] = fma(x2_0 * y2_0, z0_0, acc[19]);
+                acc[20] = fma(x2_0 * y1_0, z1_0, acc[20]);
+                acc[21] = fma(x2_0 * y0_0, z2_0, acc[21]);
+                acc[22] = fma(x1_0 * y3_0, z0_0, acc[22]);
+                acc[23] = fma(x1_0 * y2_0, z1_0, acc[23]);
+                acc[24] = fma(x1_0 * y1_0, z2_0, acc[24]);
+                acc[25] = fma(x1_0 * y0_0, z3_0, acc[25]);
+                acc[26] = fma(x0_0 * y4_0, z0_0, acc[26]);
+                acc[27] = fma(x0_0 * y3_0, z1_0, acc[27]);
+                acc[28] = fma(x0_0 * y2_0, z2_0, acc[28]);
+                acc[29] = fma(x0_0 * y1_0, z3_0, acc[29]);
+                acc[30] = fma(x0_0 * y0_0, z4_0, acc[30]);
+            }
+        }
     }
 }
 
-// grid_max: resident blocks on the device; the grid is cut to the chunks' groups.
-void launch_rys_ddss(const EriQueue &Q, const RysTab &R, int mixed, int grid_max, cudaStream_t s) {
-    if (Q.nchunks <= 0 || grid_max <= 0) return;
-    rys_prepare_ddss();
-    constexpr int ng = 128 / C_ddss::G;
-    const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    (void)mixed;  // no FP32 variant for this class
-    rys_queue_ddss<0><<<grid, 128, 15680, s>>>(Q, R);
+// Bra and ket HRR of the contracted block (src/HGP.jl:92-114), then the component norms:
+// the normalised (ab|cd) of bra pair p and ket pair q into res[36] (ma, mb, mc, md
+// row-major).
+__device__ __forceinline__ void hrr_ddss_rys(const PairTab &P, int p, int q, const double *__restrict__ acc,
+                                          double *__restrict__ res) {
+    const double4 gb = ldg4(&P.geo[p]);
+    const double4 gk = ldg4(&P.geo[q]);
+    const double ABx = gb.x, ABy = gb.y, ABz = gb.z;
+    const double CDx = gk.x, CDy = gk.y, CDz = gk.z;
+    (void)ABx; (void)ABy; (void)ABz; (void)CDx; (void)CDy; (void)CDz;
+    const double h10_1_0 = acc[16] + ABx * acc[6];
+    const double h4_1_0 = acc[6] + ABx * acc[0];
+    const double h4_4_0 = h10_1_0 + ABx * h4_1_0;
+    const double h10_2_0 = acc[17] + ABy * acc[6];
+    const double h4_2_0 = acc[7] + ABy * acc[0];
+    const double h4_5_0 = h10_2_0 + ABx * h4_2_0;
+    const double h10_3_0 = acc[18] + ABz * acc[6];
+    const double h4_3_0 = acc[8] + ABz * acc[0];
+    const double h4_6_0 = h10_3_0 + ABx * h4_3_0;
+    const double h11_2_0 = acc[19] + ABy * acc[7];
+    const double h4_7_0 = h11_2_0 + ABy * h4_2_0;
+    const double h11_3_0 = acc[20] + ABz * acc[7];
+    const double h4_8_0 = h11_3_0 + ABy * h4_3_0;
+    const double h12_3_0 = acc[21] + ABz * acc[8];
+    const double h4_9_0 = h12_3_0 + ABz * h4_3_0;
+    const double h11_1_0 = acc[17] + ABx * acc[7];
+    const double h5_1_0 = acc[7] + ABx * acc[1];
+    const double h5_4_0 = h11_1_0 + ABx * h5_1_0;
+    const double h5_2_0 = acc[9] + ABy * acc[1];
+    const double h5_5_0 = h11_2_0 + ABx * h5_2_0;
+    const double h5_3_0 = acc[11] + ABz * acc[1];
+    const double h5_6_0 = h11_3_0 + ABx * h5_3_0;
+    const double h13_2_0 = acc[22] + ABy * acc[9];
+    const double h5_7_0 = h13_2_0 + ABy * h5_2_0;
+    const double h13_3_0 = acc[23] + ABz * acc[9];
+    const double h5_8_0 = h13_3_0 + ABy * h5_3_0;
+    const double h15_3_0 = acc[24] + ABz * acc[11];
+    const double h5_9_0 = h15_3_0 + ABz * h5_3_0;
+    const double h12_1_0 = acc[18] + ABx * acc[8];
+    const double h6_1_0 = acc[8] + ABx * acc[2];
+    const double h6_4_0 = h12_1_0 + ABx * h6_1_0;
+    const double h12_2_0 = acc[20] + ABy * acc[8];
+    const double h6_2_0 = acc[11] + ABy * acc[2];
+    const double h6_5_0 = h12_2_0 + ABx * h6_2_0;
+    const double h6_3_0 = acc[10] + ABz * acc[2];
+    const double h6_6_0 = h12_3_0 + ABx * h6_3_0;
+    const double h15_2_0 = acc[23] + ABy * acc[11];
+    const double h6_7_0 = h15_2_0 + ABy * h6_2_0;
+    const double h6_8_0 = h15_3_0 + ABy * h6_3_0;
+    const double h14_3_0 = acc[25] + ABz * acc[10];
+    const double h6_9_0 = h14_3_0 + ABz * h6_3_0;
+    const double h13_1_0 = acc[19] + ABx * acc[9];
+    const double h7_1_0 = acc[9] + ABx * acc[3];
+    const double h7_4_0 = h13_1_0 + ABx * h7_1_0;
+    const double h7_2_0 = acc[12] + ABy * acc[3];
+    const double h7_5_0 = h13_2_0 + ABx * h7_2_0;
+    const double h7_3_0 = acc[13] + ABz * acc[3];
+    const double h7_6_0 = h13_3_0 + ABx * h7_3_0;
+    const double h16_2_0 = acc[26] + ABy * acc[12];
+    const double h7_7_0 = h16_2_0 + ABy * h7_2_0;
+    const double h16_3_0 = acc[27] + ABz * acc[12];
+    const double h7_8_0 = h16_3_0 + ABy * h7_3_0;
+    const double h17_3_0 = acc[28] + ABz * acc[13];
+    const double h7_9_0 = h17_3_0 + ABz * h7_3_0;
+    const double h15_1_0 = acc[20] + ABx * acc[11];
+    const double h8_1_0 = acc[11] + ABx * acc[4];
+    const double h8_4_0 = h15_1_0 + ABx * h8_1_0;
+    const double h8_2_0 = acc[13] + ABy * acc[4];
+    const double h8_5_0 = h15_2_0 + ABx * h8_2_0;
+    const double h8_3_0 = acc[14] + ABz * acc[4];
+    const double h8_6_0 = h15_3_0 + ABx * h8_3_0;
+    const double h17_2_0 = acc[27] + ABy * acc[13];
+    const double h8_7_0 = h17_2_0 + ABy * h8_2_0;
+    const double h8_8_0 = h17_3_0 + ABy * h8_3_0;
+    const double h18_3_0 = acc[29] + ABz * acc[14];
+    const double h8_9_0 = h18_3_0 + ABz * h8_3_0;
+    const double h14_1_0 = acc[21] + ABx * acc[10];
+    const double h9_1_0 = acc[10] + ABx * acc[5];
+    const double h9_4_0 = h14_1_0 + ABx * h9_1_0;
+    const double h14_2_0 = acc[24] + ABy * acc[10];
+    const double h9_2_0 = acc[14] + ABy * acc[5];
+    const double h9_5_0 = h14_2_0 + ABx * h9_2_0;
+    const double h9_3_0 = acc[15] + ABz * acc[5];
+    const double h9_6_0 = h14_3_0 + ABx * h9_3_0;
+    const double h18_2_0 = acc[28] + ABy * acc[14];
+    const double h9_7_0 = h18_2_0 + ABy * h9_2_0;
+    const double h9_8_0 = h18_3_0 + ABy * h9_3_0;
+    const double h19_3_0 = acc[30] + ABz * acc[15];
+    const double h9_9_0 = h19_3_0 + ABz * h9_3_0;
+    res[0] = h4_4_0 * 0.3333333333333334;
+    res[1] = h4_5_0 * 0.5773502691896258;
+    res[2] = h4_6_0 * 0.5773502691896258;
+    res[3] = h4_7_0 * 0.3333333333333334;
+    res[4] = h4_8_0 * 0.5773502691896258;
+    res[5] = h4_9_0 * 0.3333333333333334;
+    res[6] = h5_4_0 * 0.5773502691896258;
+    res[7] = h5_5_0;
+    res[8] = h5_6_0;
+    res[9] = h5_7_0 * 0.5773502691896258;
+    res[10] = h5_8_0;
+    res[11] = h5_9_0 * 0.5773502691896258;
+    res[12] = h6_4_0 * 0.5773502691896258;
+    res[13] = h6_5_0;
+    res[14] = h6_6_0;
+    res[15] = h6_7_0 * 0.5773502691896258;
+    res[16] = h6_8_0;
+    res[17] = h6_9_0 * 0.5773502691896258;
+    res[18] = h7_4_0 * 0.3333333333333334;
+    res[19] = h7_5_0 * 0.5773502691896258;
+    res[20] = h7_6_0 * 0.5773502691896258;
+    res[21] = h7_7_0 * 0.3333333333333334;
+    res[22] = h7_8_0 * 0.5773502691896258;
+    res[23] = h7_9_0 * 0.3333333333333334;
+    res[24] = h8_4_0 * 0.5773502691896258;
+    res[25] = h8_5_0;
+    res[26] = h8_6_0;
+    res[27] = h8_7_0 * 0.5773502691896258;
+    res[28] = h8_8_0;
+    res[29] = h8_9_0 * 0.5773502691896258;
+    res[30] = h9_4_0 * 0.3333333333333334;
+    res[31] = h9_5_0 * 0.5773502691896258;
+    res[32] = h9_6_0 * 0.5773502691896258;
+    res[33] = h9_7_0 * 0.3333333333333334;
+    res[34] = h9_8_0 * 0.5773502691896258;
+    res[35] = h9_9_0 * 0.3333333333333334;
+}
+
+
+
+__device__ __forceinline__ void store_ddss_rys(double *__restrict__ out, const int4 ib_, const int4 ik_,
+                                            bool same, const double *__restrict__ res) {
+    const bool dab = ib_.z == ib_.w, dcd = ik_.z == ik_.w;
+    (void)dab; (void)dcd;
+    const long long ij_0_0 = pair_index(ib_.z + 0, ib_.w + 0);
+    const long long ij_0_1 = pair_index(ib_.z + 0, ib_.w + 1);
+    const long long ij_0_2 = pair_index(ib_.z + 0, ib_.w + 2);
+    const long long ij_0_3 = pair_index(ib_.z + 0, ib_.w + 3);
+    const long long ij_0_4 = pair_index(ib_.z + 0, ib_.w + 4);
+    const long long ij_0_5 = pair_index(ib_.z + 0, ib_.w + 5);
+    const long long ij_1_0 = pair_index(ib_.z + 1, ib_.w + 0);
+    const long long ij_1_1 = pair_index(ib_.z + 1, ib_.w + 1);
+    const long long ij_1_2 = pair_index(ib_.z + 1, ib_.w + 2);
+    const long long ij_1_3 = pair_index(ib_.z + 1, ib_.w + 3);
+    const long long ij_1_4 = pair_index(ib_.z + 1, ib_.w + 4);
+    const long long ij_1_5 = pair_index(ib_.z + 1, ib_.w + 5);
+    const long long ij_2_0 = pair_index(ib_.z + 2, ib_.w + 0);
+    const long long ij_2_1 = pair_index(ib_.z + 2, ib_.w + 1);
+    const long long ij_2_2 = pair_index(ib_.z + 2, ib_.w + 2);
+    const long long ij_2_3 = pair_index(ib_.z + 2, ib_.w + 3);
+    const long long ij_2_4 = pair_index(ib_.z + 2, ib_.w + 4);
+    const long long ij_2_5 = pair_index(ib_.z + 2, ib_.w + 5);
+    const long long ij_3_0 = pair_index(ib_.z + 3, ib_.w + 0);
+    const long long ij_3_1 = pair_index(ib_.z + 3, ib_.w + 1);
+    const long long ij_3_2 = pair_index(ib_.z + 3, ib_.w + 2);
+    const long long ij_3_3 = pair_index(ib_.z + 3, ib_.w + 3);
+    const long long ij_3_4 = pair_index(ib_.z + 3, ib_.w + 4);
+    const long long ij_3_5 = pair_index(ib_.z + 3, ib_.w + 5);
+    const long long ij_4_0 = pair_index(ib_.z + 4, ib_.w + 0);
+    const long long ij_4_1 = pair_index(ib_.z + 4, ib_.w + 1);
+    const long long ij_4_2 = pair_index(ib_.z + 4, ib_.w + 2);
+    const long long ij_4_3 = pair_index(ib_.z + 4, ib_.w + 3);
+    const long long ij_4_4 = pair_index(ib_.z + 4, ib_.w + 4);
+    const long long ij_4_5 = pair_index(ib_.z + 4, ib_.w + 5);
+    const long long ij_5_0 = pair_index(ib_.z + 5, ib_.w + 0);
+    const long long ij_5_1 = pair_index(ib_.z + 5, ib_.w + 1);
+    const long long ij_5_2 = pair_index(ib_.z + 5, ib_.w + 2);
+    const long long ij_5_3 = pair_index(ib_.z + 5, ib_.w + 3);
+    const long long ij_5_4 = pair_index(ib_.z + 5, ib_.w + 4);
+    const long long ij_5_5 = pair_index(ib_.z + 5, ib_.w + 5);
+    const long long kl_0_0 = pair_index(ik_.z + 0, ik_.w + 0);
+    { const long long ij = ij_0_0, kl = kl_0_0;
+      if ((!dab || 0 >= 0) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[0]; }
+    { const long long ij = ij_0_1, kl = kl_0_0;
+      if ((!dab || 0 >= 1) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[1]; }
+    { const long long ij = ij_0_2, kl = kl_0_0;
+      if ((!dab || 0 >= 2) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[2]; }
+    { const long long ij = ij_0_3, kl = kl_0_0;
+      if ((!dab || 0 >= 3) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[3]; }
+    { const long long ij = ij_0_4, kl = kl_0_0;
+      if ((!dab || 0 >= 4) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[4]; }
+    { const long long ij = ij_0_5, kl = kl_0_0;
+      if ((!dab || 0 >= 5) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[5]; }
+    { const long long ij = ij_1_0, kl = kl_0_0;
+      if ((!dab || 1 >= 0) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[6]; }
+    { const long long ij = ij_1_1, kl = kl_0_0;
+      if ((!dab || 1 >= 1) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[7]; }
+    { const long long ij = ij_1_2, kl = kl_0_0;
+      if ((!dab || 1 >= 2) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[8]; }
+    { const long long ij = ij_1_3, kl = kl_0_0;
+      if ((!dab || 1 >= 3) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[9]; }
+    { const long long ij = ij_1_4, kl = kl_0_0;
+      if ((!dab || 1 >= 4) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[10]; }
+    { const long long ij = ij_1_5, kl = kl_0_0;
+      if ((!dab || 1 >= 5) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[11]; }
+    { const long long ij = ij_2_0, kl = kl_0_0;
+      if ((!dab || 2 >= 0) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[12]; }
+    { const long long ij = ij_2_1, kl = kl_0_0;
+      if ((!dab || 2 >= 1) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[13]; }
+    { const long long ij = ij_2_2, kl = kl_0_0;
+      if ((!dab || 2 >= 2) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[14]; }
+    { const long long ij = ij_2_3, kl = kl_0_0;
+      if ((!dab || 2 >= 3) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[15]; }
+    { const long long ij = ij_2_4, kl = kl_0_0;
+      if ((!dab || 2 >= 4) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[16]; }
+    { const long long ij = ij_2_5, kl = kl_0_0;
+      if ((!dab || 2 >= 5) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[17]; }
+    { const long long ij = ij_3_0, kl = kl_0_0;
+      if ((!dab || 3 >= 0) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[18]; }
+    { const long long ij = ij_3_1, kl = kl_0_0;
+      if ((!dab || 3 >= 1) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[19]; }
+    { const long long ij = ij_3_2, kl = kl_0_0;
+      if ((!dab || 3 >= 2) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[20]; }
+    { const long long ij = ij_3_3, kl = kl_0_0;
+      if ((!dab || 3 >= 3) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[21]; }
+    { const long long ij = ij_3_4, kl = kl_0_0;
+      if ((!dab || 3 >= 4) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[22]; }
+    { const long long ij = ij_3_5, kl = kl_0_0;
+      if ((!dab || 3 >= 5) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[23]; }
+    { const long long ij = ij_4_0, kl = kl_0_0;
+      if ((!dab || 4 >= 0) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[24]; }
+    { const long long ij = ij_4_1, kl = kl_0_0;
+      if ((!dab || 4 >= 1) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[25]; }
+    { const long long ij = ij_4_2, kl = kl_0_0;
+      if ((!dab || 4 >= 2) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[26]; }
+    { const long long ij = ij_4_3, kl = kl_0_0;
+      if ((!dab || 4 >= 3) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[27]; }
+    { const long long ij = ij_4_4, kl = kl_0_0;
+      if ((!dab || 4 >= 4) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[28]; }
+    { const long long ij = ij_4_5, kl = kl_0_0;
+      if ((!dab || 4 >= 5) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[29]; }
+    { const long long ij = ij_5_0, kl = kl_0_0;
+      if ((!dab || 5 >= 0) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[30]; }
+    { const long long ij = ij_5_1, kl = kl_0_0;
+      if ((!dab || 5 >= 1) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[31]; }
+    { const long long ij = ij_5_2, kl = kl_0_0;
+      if ((!dab || 5 >= 2) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[32]; }
+    { const long long ij = ij_5_3, kl = kl_0_0;
+      if ((!dab || 5 >= 3) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[33]; }
+    { const long long ij = ij_5_4, kl = kl_0_0;
+      if ((!dab || 5 >= 4) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[34]; }
+    { const long long ij = ij_5_5, kl = kl_0_0;
+      if ((!dab || 5 >= 5) && (!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[35]; }
+}
+
+// The quartet's unique integrals digested into J and K (molints_plan_jk) instead of stored.
+__device__ __noinline__ void jk_ddss_rys(const JKOut &jk, const int4 ib_, const int4 ik_, bool same,
+                                      const double *__restrict__ res) {
+    const bool dab = ib_.z == ib_.w, dcd = ik_.z == ik_.w;
+    for (int x = 0; x < 36; ++x) {
+        const int ia = x / 6, ibb = (x / 1) % 6, ic = (x / 1) % 1, id = x % 1;
+        if ((dab && ia < ibb) || (dcd && ic < id)) continue;
+        const int i = ib_.z + ia, j = ib_.w + ibb, k = ik_.z + ic, l = ik_.w + id;
+        if (same && pair_index(i, j) < pair_index(k, l)) continue;
+        jk_add(jk, i, j, k, l, res[x]);
+    }
+}
+
+// Persistent work-queue kernel: each warp takes chunks (one bra pair, a run of consecutive
+// ket pairs of one molecule) from a shared counter until the chunk list, ordered by
+// decreasing estimated cost, is exhausted.  A chunk's count field carries the split in bits
+// 16+: lg = log2 S (bits 16-18) and lgj = log2 Sj (bits 20-22).  S lanes share each quartet:
+// lane l takes ket pair q0 + l % (32/S) (+ 32/S per round); its group rank s = l / (32/S)
+// takes every Sj-th ket primitive from s % Sj and every (S/Sj)-th bra primitive from s / Sj.
+// The S partial blocks are summed by a fixed butterfly (the result depends on the split
+// alone, not on the chunk), and the group's first lane runs the HRR and stores.  Heavy
+// quartets are split so that no single lane's serial primitive loop sets the kernel time.
+// JK: digest into J and K (molints_plan_jk) instead of storing the packed integrals; a separate
+// instantiation, so that the store kernels carry none of the digestion code.
+template <int MIXED, int JK>
+__global__ void __launch_bounds__(128) eri_queue_ddss_rys(const EriQueue Q) {
+    const int lane = threadIdx.x & 31;
+    for (;;) {
+        int c = 0;
+        if (lane == 0) c = atomicAdd(Q.counter, 1);
+        c = __shfl_sync(0xffffffffu, c, 0);
+        if (c >= Q.nchunks) return;
+        const int4 ch = __ldg(&Q.chunks[c]);
+        const int p = ch.x, cnt = ch.z & 0xffff, lg = (ch.z >> 16) & 7, lgj = (ch.z >> 20) & 7;
+        const int W = 32 >> lg, kq = lane & (W - 1), s = lane >> (5 - lg);
+        const int js = s & ((1 << lgj) - 1), is = s >> lgj;
+        for (int base = 0; base < cnt; base += W) {
+        const int q = ch.y + base + kq;
+        const bool live = base + kq < cnt;
+        double acc[31];
+        double2 bp = make_double2(0.0, 0.0), bq = bp;
+        if (live) {
+            bp = __ldg(&Q.pairs.bnd[p]);
+            bq = __ldg(&Q.pairs.bnd[q]);
+        }
+        if (!live || bp.x * bq.x < Q.screen_cut) {
+#pragma unroll
+            for (int x = 0; x < 31; ++x) acc[x] = 0.0;
+        } else {
+            const int nb = __ldg(&Q.pairs.info[p]).y, nk = __ldg(&Q.pairs.info[q]).y;
+            vrr_ddss_rys(Q.pairs, Q.rys, p, q, is, nb, 1 << (lg - lgj), js, nk, 1 << lgj, acc);
+        }
+        if (lg) {
+            for (int off = W; off < 32; off <<= 1) {
+#pragma unroll
+                for (int x = 0; x < 31; ++x) acc[x] += __shfl_xor_sync(0xffffffffu, acc[x], off);
+            }
+        }
+        const bool lead = live && s == 0;
+        if (!JK && Q.scratch) {
+            // two-phase: the leaders' HRR writes the blocks of the chunk's quartets straight
+            // into shared memory, where they lie as in the scratch (consecutive slots); the warp
+            // then copies them out as one contiguous run
+            extern __shared__ double stg[];  // 4 * 32 * 36 doubles (launch_eri_ddss_rys)
+            double *sb = stg + (threadIdx.x >> 5) * (32 * 36);
+            if (lead) hrr_ddss_rys(Q.pairs, p, q, acc, sb + kq * 36);
+            __syncwarp();
+            const int nlive = min(W, cnt - base);
+            double *__restrict__ dst = Q.scratch + __ldg(&Q.region[ch.w * kRegionFields]) +
+                (__ldg(&Q.chunk_slot[c]) + base) * (long long)36;
+            for (int t = lane; t < nlive * 36; t += 32) dst[t] = sb[t];
+            __syncwarp();
+        } else if (lead) {
+            double res[36];
+            hrr_ddss_rys(Q.pairs, p, q, acc, res);
+            if constexpr (JK) {
+                jk_ddss_rys(Q.jk, __ldg(&Q.pairs.info[p]), __ldg(&Q.pairs.info[q]), p == q, res);
+            } else {
+                store_ddss_rys(Q.out + __ldg(&Q.mol_out[ch.w]), __ldg(&Q.pairs.info[p]), __ldg(&Q.pairs.info[q]),
+                            p == q, res);
+            }
+        }
+        }
+    }
+}
+
+
+void launch_rys_ddss(const EriQueue &Q0, const RysTab &R, int mixed, int grid, cudaStream_t s) {
+    EriQueue Q = Q0;
+    Q.rys = R;
+    if (Q.nchunks <= 0 || grid <= 0) return;
+    // two-phase plans stage the chunk's blocks in 36864 bytes of dynamic shared memory
+    const size_t smem = Q.scratch && !Q.jk.J ? 36864 : 0;
+    (void)mixed;  // no FP32 variant for this class (MIXED_MIN_VRR)
+    if (Q.jk.J) eri_queue_ddss_rys<0, 1><<<grid, 128, 0, s>>>(Q);
+    else eri_queue_ddss_rys<0, 0><<<grid, 128, smem, s>>>(Q);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_ddss(int mixed) {
-    rys_prepare_ddss();
+
     int n = 0;
     (void)mixed;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_ddss<0>, 128, 15680);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, eri_queue_ddss_rys<0, 0>, 128, 0);
     return n;
 }
 

@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (df|fp).  Do not edit.
-// roots 5, block 52 x 25, outputs 60 x 30, group 128 threads,
-// 13 primitive quartets per batch, 1 slot(s), 11 accumulators per thread, 47120 B shared per block.
+// roots 5, block 52 x 25, outputs 60 x 30, group 32 threads, 1 ket pairs a round,
+// 6 primitive quartets per ket pair and batch, 107520 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,177 +11,412 @@ struct C_dffp {
     static constexpr int NA = 52, NC = 25, NBLK = 1300;
     static constexpr int NB = 10, ND = 3;
     static constexpr int NAB = 60, NCD = 30;
-    static constexpr int G = 128, NPB = 13, NSLOT = 1, ACC = 11;
-    static constexpr int S = 30;
-    static constexpr int SMEM_GROUP = 5890;
-    static constexpr bool COL = false;
+    static constexpr int G = 32, W = 1, H = 1, PB = 6;
+    static constexpr int S = 30, SI = 91, NCP = 25, NCDP = 31;
+    static constexpr int SMEM_GROUP = 3360;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
-    __device__ __forceinline__ static void col_update(const T *, const T *, const T *, A *) {}
+    __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
+        acc[0] = fma(x[2] * y[0], z[0], acc[0]);
+        acc[1] = fma(x[1] * y[1], z[0], acc[1]);
+        acc[2] = fma(x[1] * y[0], z[1], acc[2]);
+        acc[3] = fma(x[0] * y[2], z[0], acc[3]);
+        acc[4] = fma(x[0] * y[1], z[1], acc[4]);
+        acc[5] = fma(x[0] * y[0], z[2], acc[5]);
+        acc[6] = fma(x[3] * y[0], z[0], acc[6]);
+        acc[7] = fma(x[2] * y[1], z[0], acc[7]);
+        acc[8] = fma(x[2] * y[0], z[1], acc[8]);
+        acc[9] = fma(x[1] * y[2], z[0], acc[9]);
+        acc[10] = fma(x[1] * y[0], z[2], acc[10]);
+        acc[11] = fma(x[1] * y[1], z[1], acc[11]);
+        acc[12] = fma(x[0] * y[3], z[0], acc[12]);
+        acc[13] = fma(x[0] * y[2], z[1], acc[13]);
+        acc[14] = fma(x[0] * y[1], z[2], acc[14]);
+        acc[15] = fma(x[0] * y[0], z[3], acc[15]);
+        acc[16] = fma(x[4] * y[0], z[0], acc[16]);
+        acc[17] = fma(x[3] * y[1], z[0], acc[17]);
+        acc[18] = fma(x[3] * y[0], z[1], acc[18]);
+        acc[19] = fma(x[2] * y[2], z[0], acc[19]);
+        acc[20] = fma(x[2] * y[1], z[1], acc[20]);
+        acc[21] = fma(x[2] * y[0], z[2], acc[21]);
+        acc[22] = fma(x[1] * y[3], z[0], acc[22]);
+        acc[23] = fma(x[1] * y[2], z[1], acc[23]);
+        acc[24] = fma(x[1] * y[1], z[2], acc[24]);
+        acc[25] = fma(x[1] * y[0], z[3], acc[25]);
+        acc[26] = fma(x[0] * y[4], z[0], acc[26]);
+        acc[27] = fma(x[0] * y[3], z[1], acc[27]);
+        acc[28] = fma(x[0] * y[2], z[2], acc[28]);
+        acc[29] = fma(x[0] * y[1], z[3], acc[29]);
+        acc[30] = fma(x[0] * y[0], z[4], acc[30]);
+        acc[31] = fma(x[5] * y[0], z[0], acc[31]);
+        acc[32] = fma(x[4] * y[1], z[0], acc[32]);
+        acc[33] = fma(x[4] * y[0], z[1], acc[33]);
+        acc[34] = fma(x[3] * y[2], z[0], acc[34]);
+        acc[35] = fma(x[3] * y[1], z[1], acc[35]);
+        acc[36] = fma(x[3] * y[0], z[2], acc[36]);
+        acc[37] = fma(x[2] * y[3], z[0], acc[37]);
+        acc[38] = fma(x[2] * y[2], z[1], acc[38]);
+        acc[39] = fma(x[2] * y[1], z[2], acc[39]);
+        acc[40] = fma(x[2] * y[0], z[3], acc[40]);
+        acc[41] = fma(x[1] * y[4], z[0], acc[41]);
+        acc[42] = fma(x[1] * y[3], z[1], acc[42]);
+        acc[43] = fma(x[1] * y[2], z[2], acc[43]);
+        acc[44] = fma(x[1] * y[1], z[3], acc[44]);
+        acc[45] = fma(x[1] * y[0], z[4], acc[45]);
+        acc[46] = fma(x[0] * y[5], z[0], acc[46]);
+        acc[47] = fma(x[0] * y[4], z[1], acc[47]);
+        acc[48] = fma(x[0] * y[3], z[2], acc[48]);
+        acc[49] = fma(x[0] * y[2], z[3], acc[49]);
+        acc[50] = fma(x[0] * y[1], z[4], acc[50]);
+        acc[51] = fma(x[0] * y[0], z[5], acc[51]);
+    }
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[16], in[31]);
+        const double h1 = fma(x, in[6], in[16]);
+        const double h2 = fma(x, h1, h0);
+        const double h3 = fma(x, in[0], in[6]);
+        const double h4 = fma(x, h3, h1);
+        const double h5 = fma(x, h4, h2);
+        const double h6 = fma(y, in[16], in[32]);
+        const double h7 = fma(y, in[6], in[17]);
+        const double h8 = fma(x, h7, h6);
+        const double h9 = fma(y, in[0], in[7]);
+        const double h10 = fma(x, h9, h7);
+        const double h11 = fma(x, h10, h8);
+        const double h12 = fma(z, in[16], in[33]);
+        const double h13 = fma(z, in[6], in[18]);
+        const double h14 = fma(x, h13, h12);
+        const double h15 = fma(z, in[0], in[8]);
+        const double h16 = fma(x, h15, h13);
+        const double h17 = fma(x, h16, h14);
+        const double h18 = fma(y, in[17], in[34]);
+        const double h19 = fma(y, in[7], in[19]);
+        const double h20 = fma(x, h19, h18);
+        const double h21 = fma(y, h10, h20);
+        const double h22 = fma(z, in[18], in[36]);
+        const double h23 = fma(z, in[8], in[21]);
+        const double h24 = fma(x, h23, h22);
+        const double h25 = fma(z, h16, h24);
+        const double h26 = fma(z, in[17], in[35]);
+        const double h27 = fma(y, h13, h26);
+        const double h28 = fma(z, in[7], in[20]);
+        const double h29 = fma(y, h15, h28);
+        const double h30 = fma(x, h29, h27);
+        const double h31 = fma(y, in[19], in[37]);
+        const double h32 = fma(y, h19, h31);
+        const double h33 = fma(y, h9, h19);
+        const double h34 = fma(y, h33, h32);
+        const double h35 = fma(z, in[19], in[38]);
+        const double h36 = fma(y, h28, h35);
+        const double h37 = fma(y, h29, h36);
+        const double h38 = fma(z, in[20], in[39]);
+        const double h39 = fma(y, h23, h38);
+        const double h40 = fma(z, h29, h39);
+        const double h41 = fma(z, in[21], in[40]);
+        const double h42 = fma(z, h23, h41);
+        const double h43 = fma(z, h15, h23);
+        const double h44 = fma(z, h43, h42);
+        const double h45 = fma(x, in[17], in[32]);
+        const double h46 = fma(x, in[7], in[17]);
+        const double h47 = fma(x, h46, h45);
+        const double h48 = fma(x, in[1], in[7]);
+        const double h49 = fma(x, h48, h46);
+        const double h50 = fma(x, h49, h47);
+        const double h51 = fma(y, in[1], in[9]);
+        const double h52 = fma(x, h51, h19);
+        const double h53 = fma(x, h52, h20);
+        const double h54 = fma(x, h28, h26);
+        const double h55 = fma(z, in[1], in[11]);
+        const double h56 = fma(x, h55, h28);
+        const double h57 = fma(x, h56, h54);
+        const double h58 = fma(y, in[9], in[22]);
+        const double h59 = fma(x, h58, h31);
+        const double h60 = fma(y, h52, h59);
+        const double h61 = fma(z, in[11], in[24]);
+        const double h62 = fma(x, h61, h38);
+        const double h63 = fma(z, h56, h62);
+        const double h64 = fma(z, in[9], in[23]);
+        const double h65 = fma(y, h55, h64);
+        const double h66 = fma(x, h65, h36);
+        const double h67 = fma(y, in[22], in[41]);
+        const double h68 = fma(y, h58, h67);
+        const double h69 = fma(y, h51, h58);
+        const double h70 = fma(y, h69, h68);
+        const double h71 = fma(z, in[22], in[42]);
+        const double h72 = fma(y, h64, h71);
+        const double h73 = fma(y, h65, h72);
+        const double h74 = fma(z, in[23], in[43]);
+        const double h75 = fma(y, h61, h74);
+        const double h76 = fma(z, h65, h75);
+        const double h77 = fma(z, in[24], in[44]);
+        const double h78 = fma(z, h61, h77);
+        const double h79 = fma(z, h55, h61);
+        const double h80 = fma(z, h79, h78);
+        const double h81 = fma(x, in[18], in[33]);
+        const double h82 = fma(x, in[8], in[18]);
+        const double h83 = fma(x, h82, h81);
+        const double h84 = fma(x, in[2], in[8]);
+        const double h85 = fma(x, h84, h82);
+        const double h86 = fma(x, h85, h83);
+        const double h87 = fma(y, in[18], in[35]);
+        const double h88 = fma(y, in[8], in[20]);
+        const double h89 = fma(x, h88, h87);
+        const double h90 = fma(y, in[2], in[11]);
+        const double h91 = fma(x, h90, h88);
+        const double h92 = fma(x, h91, h89);
+        const double h93 = fma(z, in[2], in[10]);
+        const double h94 = fma(x, h93, h23);
+        const double h95 = fma(x, h94, h24);
+        const double h96 = fma(y, in[20], in[38]);
+        const double h97 = fma(y, in[11], in[23]);
+        const double h98 = fma(x, h97, h96);
+        const double h99 = fma(y, h91, h98);
+        const double h100 = fma(z, in[10], in[25]);
+        const double h101 = fma(x, h100, h41);
+        const double h102 = fma(z, h94, h101);
+        const double h103 = fma(y, h93, h61);
+        const double h104 = fma(x, h103, h39);
+        const double h105 = fma(y, in[23], in[42]);
+        const double h106 = fma(y, h97, h105);
+        const double h107 = fma(y, h90, h97);
+        const double h108 = fma(y, h107, h106);
+        const double h109 = fma(y, h103, h75);
+        const double h110 = fma(y, h100, h77);
+        const double h111 = fma(z, h103, h110);
+        const double h112 = fma(z, in[25], in[45]);
+        const double h113 = fma(z, h100, h112);
+        const double h114 = fma(z, h93, h100);
+        const double h115 = fma(z, h114, h113);
+        const double h116 = fma(x, in[19], in[34]);
+        const double h117 = fma(x, in[9], in[19]);
+        const double h118 = fma(x, h117, h116);
+        const double h119 = fma(x, in[3], in[9]);
+        const double h120 = fma(x, h119, h117);
+        const double h121 = fma(x, h120, h118);
+        const double h122 = fma(y, in[3], in[12]);
+        const double h123 = fma(x, h122, h58);
+        const double h124 = fma(x, h123, h59);
+        const double h125 = fma(x, h64, h35);
+        const double h126 = fma(z, in[3], in[13]);
+        const double h127 = fma(x, h126, h64);
+        const double h128 = fma(x, h127, h125);
+        const double h129 = fma(y, in[12], in[26]);
+        const double h130 = fma(x, h129, h67);
+        const double h131 = fma(y, h123, h130);
+        const double h132 = fma(z, in[13], in[28]);
+        const double h133 = fma(x, h132, h74);
+        const double h134 = fma(z, h127, h133);
+        const double h135 = fma(z, in[12], in[27]);
+        const double h136 = fma(y, h126, h135);
+        const double h137 = fma(x, h136, h72);
+        const double h138 = fma(y, in[26], in[46]);
+        const double h139 = fma(y, h129, h138);
+        const double h140 = fma(y, h122, h129);
+        const double h141 = fma(y, h140, h139);
+        const double h142 = fma(z, in[26], in[47]);
+        const double h143 = fma(y, h135, h142);
+        const double h144 = fma(y, h136, h143);
+        const double h145 = fma(z, in[27], in[48]);
+        const double h146 = fma(y, h132, h145);
+        const double h147 = fma(z, h136, h146);
+        const double h148 = fma(z, in[28], in[49]);
+        const double h149 = fma(z, h132, h148);
+        const double h150 = fma(z, h126, h132);
+        const double h151 = fma(z, h150, h149);
+        const double h152 = fma(x, in[20], in[35]);
+        const double h153 = fma(x, in[11], in[20]);
+        const double h154 = fma(x, h153, h152);
+        const double h155 = fma(x, in[4], in[11]);
+        const double h156 = fma(x, h155, h153);
+        const double h157 = fma(x, h156, h154);
+        const double h158 = fma(y, in[4], in[13]);
+        const double h159 = fma(x, h158, h97);
+        const double h160 = fma(x, h159, h98);
+        const double h161 = fma(z, in[4], in[14]);
+        const double h162 = fma(x, h161, h61);
+        const double h163 = fma(x, h162, h62);
+        const double h164 = fma(y, in[13], in[27]);
+        const double h165 = fma(x, h164, h105);
+        const double h166 = fma(y, h159, h165);
+        const double h167 = fma(z, in[14], in[29]);
+        const double h168 = fma(x, h167, h77);
+        const double h169 = fma(z, h162, h168);
+        const double h170 = fma(y, h161, h132);
+        const double h171 = fma(x, h170, h75);
+        const double h172 = fma(y, in[27], in[47]);
+        const double h173 = fma(y, h164, h172);
+        const double h174 = fma(y, h158, h164);
+        const double h175 = fma(y, h174, h173);
+        const double h176 = fma(y, h170, h146);
+        const double h177 = fma(y, h167, h148);
+        const double h178 = fma(z, h170, h177);
+        const double h179 = fma(z, in[29], in[50]);
+        const double h180 = fma(z, h167, h179);
+        const double h181 = fma(z, h161, h167);
+        const double h182 = fma(z, h181, h180);
+        const double h183 = fma(x, in[21], in[36]);
+        const double h184 = fma(x, in[10], in[21]);
+        const double h185 = fma(x, h184, h183);
+        const double h186 = fma(x, in[5], in[10]);
+        const double h187 = fma(x, h186, h184);
+        const double h188 = fma(x, h187, h185);
+        const double h189 = fma(y, in[21], in[39]);
+        const double h190 = fma(y, in[10], in[24]);
+        const double h191 = fma(x, h190, h189);
+        const double h192 = fma(y, in[5], in[14]);
+        const double h193 = fma(x, h192, h190);
+        const double h194 = fma(x, h193, h191);
+        const double h195 = fma(z, in[5], in[15]);
+        const double h196 = fma(x, h195, h100);
+        const double h197 = fma(x, h196, h101);
+        const double h198 = fma(y, in[24], in[43]);
+        const double h199 = fma(y, in[14], in[28]);
+        const double h200 = fma(x, h199, h198);
+        const double h201 = fma(y, h193, h200);
+        const double h202 = fma(z, in[15], in[30]);
+        const double h203 = fma(x, h202, h112);
+        const double h204 = fma(z, h196, h203);
+        const double h205 = fma(y, h195, h167);
+        const double h206 = fma(x, h205, h110);
+        const double h207 = fma(y, in[28], in[48]);
+        const double h208 = fma(y, h199, h207);
+        const double h209 = fma(y, h192, h199);
+        const double h210 = fma(y, h209, h208);
+        const double h211 = fma(y, h205, h177);
+        const double h212 = fma(y, h202, h179);
+        const double h213 = fma(z, h205, h212);
+        const double h214 = fma(z, in[30], in[51]);
+        const double h215 = fma(z, h202, h214);
+        const double h216 = fma(z, h195, h202);
+        const double h217 = fma(z, h216, h215);
+        out[0] = h5;
+        out[25] = h11;
+        out[50] = h17;
+        out[75] = h21;
+        out[100] = h25;
+        out[125] = h30;
+        out[150] = h34;
+        out[175] = h37;
+        out[200] = h40;
+        out[225] = h44;
+        out[250] = h50;
+        out[275] = h53;
+        out[300] = h57;
+        out[325] = h60;
+        out[350] = h63;
+        out[375] = h66;
+        out[400] = h70;
+        out[425] = h73;
+        out[450] = h76;
+        out[475] = h80;
+        out[500] = h86;
+        out[525] = h92;
+        out[550] = h95;
+        out[575] = h99;
+        out[600] = h102;
+        out[625] = h104;
+        out[650] = h108;
+        out[675] = h109;
+        out[700] = h111;
+        out[725] = h115;
+        out[750] = h121;
+        out[775] = h124;
+        out[800] = h128;
+        out[825] = h131;
+        out[850] = h134;
+        out[875] = h137;
+        out[900] = h141;
+        out[925] = h144;
+        out[950] = h147;
+        out[975] = h151;
+        out[1000] = h157;
+        out[1025] = h160;
+        out[1050] = h163;
+        out[1075] = h166;
+        out[1100] = h169;
+        out[1125] = h171;
+        out[1150] = h175;
+        out[1175] = h176;
+        out[1200] = h178;
+        out[1225] = h182;
+        out[1250] = h188;
+        out[1275] = h194;
+        out[1300] = h197;
+        out[1325] = h201;
+        out[1350] = h204;
+        out[1375] = h206;
+        out[1400] = h210;
+        out[1425] = h211;
+        out[1450] = h213;
+        out[1475] = h217;
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[0], in[10]);
+        const double h1 = fma(y, in[0], in[11]);
+        const double h2 = fma(z, in[0], in[12]);
+        const double h3 = fma(x, in[1], in[11]);
+        const double h4 = fma(y, in[1], in[13]);
+        const double h5 = fma(z, in[1], in[14]);
+        const double h6 = fma(x, in[2], in[12]);
+        const double h7 = fma(y, in[2], in[14]);
+        const double h8 = fma(z, in[2], in[15]);
+        const double h9 = fma(x, in[3], in[13]);
+        const double h10 = fma(y, in[3], in[16]);
+        const double h11 = fma(z, in[3], in[17]);
+        const double h12 = fma(x, in[4], in[15]);
+        const double h13 = fma(y, in[4], in[18]);
+        const double h14 = fma(z, in[4], in[19]);
+        const double h15 = fma(x, in[5], in[14]);
+        const double h16 = fma(y, in[5], in[17]);
+        const double h17 = fma(z, in[5], in[18]);
+        const double h18 = fma(x, in[6], in[16]);
+        const double h19 = fma(y, in[6], in[20]);
+        const double h20 = fma(z, in[6], in[21]);
+        const double h21 = fma(x, in[7], in[17]);
+        const double h22 = fma(y, in[7], in[21]);
+        const double h23 = fma(z, in[7], in[22]);
+        const double h24 = fma(x, in[8], in[18]);
+        const double h25 = fma(y, in[8], in[22]);
+        const double h26 = fma(z, in[8], in[23]);
+        const double h27 = fma(x, in[9], in[19]);
+        const double h28 = fma(y, in[9], in[23]);
+        const double h29 = fma(z, in[9], in[24]);
+        out[0] = h0 * (nrm * 0.2581988897471611);
+        out[1] = h1 * (nrm * 0.2581988897471611);
+        out[2] = h2 * (nrm * 0.2581988897471611);
+        out[3] = h3 * (nrm * 0.5773502691896258);
+        out[4] = h4 * (nrm * 0.5773502691896258);
+        out[5] = h5 * (nrm * 0.5773502691896258);
+        out[6] = h6 * (nrm * 0.5773502691896258);
+        out[7] = h7 * (nrm * 0.5773502691896258);
+        out[8] = h8 * (nrm * 0.5773502691896258);
+        out[9] = h9 * (nrm * 0.5773502691896258);
+        out[10] = h10 * (nrm * 0.5773502691896258);
+        out[11] = h11 * (nrm * 0.5773502691896258);
+        out[12] = h12 * (nrm * 0.5773502691896258);
+        out[13] = h13 * (nrm * 0.5773502691896258);
+        out[14] = h14 * (nrm * 0.5773502691896258);
+        out[15] = h15 * (nrm * 1.0);
+        out[16] = h16 * (nrm * 1.0);
+        out[17] = h17 * (nrm * 1.0);
+        out[18] = h18 * (nrm * 0.2581988897471611);
+        out[19] = h19 * (nrm * 0.2581988897471611);
+        out[20] = h20 * (nrm * 0.2581988897471611);
+        out[21] = h21 * (nrm * 0.5773502691896258);
+        out[22] = h22 * (nrm * 0.5773502691896258);
+        out[23] = h23 * (nrm * 0.5773502691896258);
+        out[24] = h24 * (nrm * 0.5773502691896258);
+        out[25] = h25 * (nrm * 0.5773502691896258);
+        out[26] = h26 * (nrm * 0.5773502691896258);
+        out[27] = h27 * (nrm * 0.2581988897471611);
+        out[28] = h28 * (nrm * 0.2581988897471611);
+        out[29] = h29 * (nrm * 0.2581988897471611);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_dffp[1300] = {
-    13, 268, 65548, 523, 131083, 65803, 778, 66058, 131338, 196618, 14, 269,
-    65549, 524, 65804, 131084, 779, 66059, 131339, 196619, 1034, 66314, 131594, 196874,
-    262154, 1288, 1543, 66823, 1798, 132358, 67078, 2053, 67333, 132613, 197893, 1289,
-    1544, 66824, 1799, 67079, 132359, 2054, 67334, 132614, 197894, 2309, 67589, 132869,
-    198149, 263429, 327688, 327943, 393223, 328198, 458758, 393478, 328453, 393733, 459013, 524293,
-    327689, 327944, 393224, 328199, 393479, 458759, 328454, 393734, 459014, 524294, 328709, 393989,
-    459269, 524549, 589829, 2563, 2818, 68098, 3073, 133633, 68353, 3328, 68608, 133888,
-    199168, 2564, 2819, 68099, 3074, 68354, 133634, 3329, 68609, 133889, 199169, 3584,
-    68864, 134144, 199424, 264704, 328963, 329218, 394498, 329473, 460033, 394753, 329728, 395008,
-    460288, 525568, 328964, 329219, 394499, 329474, 394754, 460034, 329729, 395009, 460289, 525569,
-    329984, 395264, 460544, 525824, 591104, 655363, 655618, 720898, 655873, 786433, 721153, 656128,
-    721408, 786688, 851968, 655364, 655619, 720899, 655874, 721154, 786434, 656129, 721409, 786689,
-    851969, 656384, 721664, 786944, 852224, 917504, 18, 273, 65553, 528, 131088, 65808,
-    783, 66063, 131343, 196623, 19, 274, 65554, 529, 65809, 131089, 784, 66064,
-    131344, 196624, 1039, 66319, 131599, 196879, 262159, 1293, 1548, 66828, 1803, 132363,
-    67083, 2058, 67338, 132618, 197898, 1294, 1549, 66829, 1804, 67084, 132364, 2059,
-    67339, 132619, 197899, 2314, 67594, 132874, 198154, 263434, 327693, 327948, 393228, 328203,
-    458763, 393483, 328458, 393738, 459018, 524298, 327694, 327949, 393229, 328204, 393484, 458764,
-    328459, 393739, 459019, 524299, 328714, 393994, 459274, 524554, 589834, 2568, 2823, 68103,
-    3078, 133638, 68358, 3333, 68613, 133893, 199173, 2569, 2824, 68104, 3079, 68359,
-    133639, 3334, 68614, 133894, 199174, 3589, 68869, 134149, 199429, 264709, 655368, 655623,
-    720903, 655878, 786438, 721158, 656133, 721413, 786693, 851973, 655369, 655624, 720904, 655879,
-    721159, 786439, 656134, 721414, 786694, 851974, 656389, 721669, 786949, 852229, 917509, 328968,
-    329223, 394503, 329478, 460038, 394758, 329733, 395013, 460293, 525573, 328969, 329224, 394504,
-    329479, 394759, 460039, 329734, 395014, 460294, 525574, 329989, 395269, 460549, 525829, 591109,
-    3843, 4098, 69378, 4353, 134913, 69633, 4608, 69888, 135168, 200448, 3844, 4099,
-    69379, 4354, 69634, 134914, 4609, 69889, 135169, 200449, 4864, 70144, 135424, 200704,
-    265984, 330243, 330498, 395778, 330753, 461313, 396033, 331008, 396288, 461568, 526848, 330244,
-    330499, 395779, 330754, 396034, 461314, 331009, 396289, 461569, 526849, 331264, 396544, 461824,
-    527104, 592384, 656643, 656898, 722178, 657153, 787713, 722433, 657408, 722688, 787968, 853248,
-    656644, 656899, 722179, 657154, 722434, 787714, 657409, 722689, 787969, 853249, 657664, 722944,
-    788224, 853504, 918784, 983043, 983298, 1048578, 983553, 1114113, 1048833, 983808, 1049088, 1114368,
-    1179648, 983044, 983299, 1048579, 983554, 1048834, 1114114, 983809, 1049089, 1114369, 1179649, 984064,
-    1049344, 1114624, 1179904, 1245184, 23, 278, 65558, 533, 131093, 65813, 788, 66068,
-    131348, 196628, 24, 279, 65559, 534, 65814, 131094, 789, 66069, 131349, 196629,
-    1044, 66324, 131604, 196884, 262164, 1298, 1553, 66833, 1808, 132368, 67088, 2063,
-    67343, 132623, 197903, 1299, 1554, 66834, 1809, 67089, 132369, 2064, 67344, 132624,
-    197904, 2319, 67599, 132879, 198159, 263439, 327698, 327953, 393233, 328208, 458768, 393488,
-    328463, 393743, 459023, 524303, 327699, 327954, 393234, 328209, 393489, 458769, 328464, 393744,
-    459024, 524304, 328719, 393999, 459279, 524559, 589839, 2573, 2828, 68108, 3083, 133643,
-    68363, 3338, 68618, 133898, 199178, 2574, 2829, 68109, 3084, 68364, 133644, 3339,
-    68619, 133899, 199179, 3594, 68874, 134154, 199434, 264714, 328973, 329228, 394508, 329483,
-    460043, 394763, 329738, 395018, 460298, 525578, 328974, 329229, 394509, 329484, 394764, 460044,
-    329739, 395019, 460299, 525579, 329994, 395274, 460554, 525834, 591114, 655373, 655628, 720908,
-    655883, 786443, 721163, 656138, 721418, 786698, 851978, 655374, 655629, 720909, 655884, 721164,
-    786444, 656139, 721419, 786699, 851979, 656394, 721674, 786954, 852234, 917514, 3848, 4103,
-    69383, 4358, 134918, 69638, 4613, 69893, 135173, 200453, 3849, 4104, 69384, 4359,
-    69639, 134919, 4614, 69894, 135174, 200454, 4869, 70149, 135429, 200709, 265989, 330248,
-    330503, 395783, 330758, 461318, 396038, 331013, 396293, 461573, 526853, 330249, 330504, 395784,
-    330759, 396039, 461319, 331014, 396294, 461574, 526854, 331269, 396549, 461829, 527109, 592389,
-    656648, 656903, 722183, 657158, 787718, 722438, 657413, 722693, 787973, 853253, 656649, 656904,
-    722184, 657159, 722439, 787719, 657414, 722694, 787974, 853254, 657669, 722949, 788229, 853509,
-    918789, 983048, 983303, 1048583, 983558, 1114118, 1048838, 983813, 1049093, 1114373, 1179653, 983049,
-    983304, 1048584, 983559, 1048839, 1114119, 983814, 1049094, 1114374, 1179654, 984069, 1049349, 1114629,
-    1179909, 1245189, 5123, 5378, 70658, 5633, 136193, 70913, 5888, 71168, 136448, 201728,
-    5124, 5379, 70659, 5634, 70914, 136194, 5889, 71169, 136449, 201729, 6144, 71424,
-    136704, 201984, 267264, 331523, 331778, 397058, 332033, 462593, 397313, 332288, 397568, 462848,
-    528128, 331524, 331779, 397059, 332034, 397314, 462594, 332289, 397569, 462849, 528129, 332544,
-    397824, 463104, 528384, 593664, 657923, 658178, 723458, 658433, 788993, 723713, 658688, 723968,
-    789248, 854528, 657924, 658179, 723459, 658434, 723714, 788994, 658689, 723969, 789249, 854529,
-    658944, 724224, 789504, 854784, 920064, 984323, 984578, 1049858, 984833, 1115393, 1050113, 985088,
-    1050368, 1115648, 1180928, 984324, 984579, 1049859, 984834, 1050114, 1115394, 985089, 1050369, 1115649,
-    1180929, 985344, 1050624, 1115904, 1181184, 1246464, 1310723, 1310978, 1376258, 1311233, 1441793, 1376513,
-    1311488, 1376768, 1442048, 1507328, 1310724, 1310979, 1376259, 1311234, 1376514, 1441794, 1311489, 1376769,
-    1442049, 1507329, 1311744, 1377024, 1442304, 1507584, 1572864, 28, 283, 65563, 538, 131098,
-    65818, 793, 66073, 131353, 196633, 29, 284, 65564, 539, 65819, 131099, 794,
-    66074, 131354, 196634, 1049, 66329, 131609, 196889, 262169, 1303, 1558, 66838, 1813,
-    132373, 67093, 2068, 67348, 132628, 197908, 1304, 1559, 66839, 1814, 67094, 132374,
-    2069, 67349, 132629, 197909, 2324, 67604, 132884, 198164, 263444, 327703, 327958, 393238,
-    328213, 458773, 393493, 328468, 393748, 459028, 524308, 327704, 327959, 393239, 328214, 393494,
-    458774, 328469, 393749, 459029, 524309, 328724, 394004, 459284, 524564, 589844, 2578, 2833,
-    68113, 3088, 133648, 68368, 3343, 68623, 133903, 199183, 2579, 2834, 68114, 3089,
-    68369, 133649, 3344, 68624, 133904, 199184, 3599, 68879, 134159, 199439, 264719, 328978,
-    329233, 394513, 329488, 460048, 394768, 329743, 395023, 460303, 525583, 328979, 329234, 394514,
-    329489, 394769, 460049, 329744, 395024, 460304, 525584, 329999, 395279, 460559, 525839, 591119,
-    655378, 655633, 720913, 655888, 786448, 721168, 656143, 721423, 786703, 851983, 655379, 655634,
-    720914, 655889, 721169, 786449, 656144, 721424, 786704, 851984, 656399, 721679, 786959, 852239,
-    917519, 3853, 4108, 69388, 4363, 134923, 69643, 4618, 69898, 135178, 200458, 3854,
-    4109, 69389, 4364, 69644, 134924, 4619, 69899, 135179, 200459, 4874, 70154, 135434,
-    200714, 265994, 330253, 330508, 395788, 330763, 461323, 396043, 331018, 396298, 461578, 526858,
-    330254, 330509, 395789, 330764, 396044, 461324, 331019, 396299, 461579, 526859, 331274, 396554,
-    461834, 527114, 592394, 656653, 656908, 722188, 657163, 787723, 722443, 657418, 722698, 787978,
-    853258, 656654, 656909, 722189, 657164, 722444, 787724, 657419, 722699, 787979, 853259, 657674,
-    722954, 788234, 853514, 918794, 983053, 983308, 1048588, 983563, 1114123, 1048843, 983818, 1049098,
-    1114378, 1179658, 983054, 983309, 1048589, 983564, 1048844, 1114124, 983819, 1049099, 1114379, 1179659,
-    984074, 1049354, 1114634, 1179914, 1245194, 5128, 5383, 70663, 5638, 136198, 70918, 5893,
-    71173, 136453, 201733, 5129, 5384, 70664, 5639, 70919, 136199, 5894, 71174, 136454,
-    201734, 6149, 71429, 136709, 201989, 267269, 331528, 331783, 397063, 332038, 462598, 397318,
-    332293, 397573, 462853, 528133, 331529, 331784, 397064, 332039, 397319, 462599, 332294, 397574,
-    462854, 528134, 332549, 397829, 463109, 528389, 593669, 657928, 658183, 723463, 658438, 788998,
-    723718, 658693, 723973, 789253, 854533, 657929, 658184, 723464, 658439, 723719, 788999, 658694,
-    723974, 789254, 854534, 658949, 724229, 789509, 854789, 920069, 984328, 984583, 1049863, 984838,
-    1115398, 1050118, 985093, 1050373, 1115653, 1180933, 984329, 984584, 1049864, 984839, 1050119, 1115399,
-    985094, 1050374, 1115654, 1180934, 985349, 1050629, 1115909, 1181189, 1246469, 1310728, 1310983, 1376263,
-    1311238, 1441798, 1376518, 1311493, 1376773, 1442053, 1507333, 1310729, 1310984, 1376264, 1311239, 1376519,
-    1441799, 1311494, 1376774, 1442054, 1507334, 1311749, 1377029, 1442309, 1507589, 1572869, 6403, 6658,
-    71938, 6913, 137473, 72193, 7168, 72448, 137728, 203008, 6404, 6659, 71939, 6914,
-    72194, 137474, 7169, 72449, 137729, 203009, 7424, 72704, 137984, 203264, 268544, 332803,
-    333058, 398338, 333313, 463873, 398593, 333568, 398848, 464128, 529408, 332804, 333059, 398339,
-    333314, 398594, 463874, 333569, 398849, 464129, 529409, 333824, 399104, 464384, 529664, 594944,
-    659203, 659458, 724738, 659713, 790273, 724993, 659968, 725248, 790528, 855808, 659204, 659459,
-    724739, 659714, 724994, 790274, 659969, 725249, 790529, 855809, 660224, 725504, 790784, 856064,
-    921344, 985603, 985858, 1051138, 986113, 1116673, 1051393, 986368, 1051648, 1116928, 1182208, 985604,
-    985859, 1051139, 986114, 1051394, 1116674, 986369, 1051649, 1116929, 1182209, 986624, 1051904, 1117184,
-    1182464, 1247744, 1312003, 1312258, 1377538, 1312513, 1443073, 1377793, 1312768, 1378048, 1443328, 1508608,
-    1312004, 1312259, 1377539, 1312514, 1377794, 1443074, 1312769, 1378049, 1443329, 1508609, 1313024, 1378304,
-    1443584, 1508864, 1574144, 1638403, 1638658, 1703938, 1638913, 1769473, 1704193, 1639168, 1704448, 1769728,
-    1835008, 1638404, 1638659, 1703939, 1638914, 1704194, 1769474, 1639169, 1704449, 1769729, 1835009, 1639424,
-    1704704, 1769984, 1835264, 1900544,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_dffp[61] = {
-    0, 4, 10, 16, 22, 28, 36, 40, 46, 52, 56, 60,
-    66, 72, 78, 84, 92, 96, 102, 108, 112, 116, 122, 128,
-    134, 140, 148, 152, 158, 164, 168, 172, 178, 184, 190, 196,
-    204, 208, 214, 220, 224, 228, 234, 240, 246, 252, 260, 264,
-    270, 276, 280, 284, 290, 296, 302, 308, 316, 320, 326, 332,
-    336,
-};
-__device__ const uint32_t kBraTerm_dffp[336] = {
-    68096, 197638, 196880, 65567, 68352, 66567, 132358, 131345, 66064, 65568, 68608, 66568,
-    132614, 131346, 66320, 65569, 68864, 132359, 65811, 67334, 131601, 65570, 69376, 132616,
-    65813, 67846, 131858, 65572, 69120, 66824, 67079, 65812, 67590, 66066, 66321, 65571,
-    69632, 198407, 197139, 65573, 69888, 67336, 133127, 131604, 66323, 65574, 70144, 133128,
-    66069, 67847, 131860, 65575, 70400, 198920, 197397, 65576, 68097, 197639, 196881, 65568,
-    68353, 66569, 132359, 131347, 66065, 65570, 68609, 66571, 132615, 131348, 66321, 65571,
-    68865, 132361, 65814, 67335, 131603, 65573, 69377, 132619, 65816, 67847, 131860, 65575,
-    69121, 66827, 67081, 65815, 67591, 66068, 66323, 65574, 69633, 198409, 197142, 65577,
-    69889, 67339, 133129, 131607, 66326, 65578, 70145, 133131, 66072, 67849, 131863, 65579,
-    70401, 198923, 197400, 65580, 68098, 197640, 196882, 65569, 68354, 66571, 132360, 131348,
-    66066, 65571, 68610, 66570, 132616, 131349, 66322, 65572, 68866, 132363, 65815, 67336,
-    131604, 65574, 69378, 132618, 65817, 67848, 131861, 65576, 69122, 66826, 67083, 65816,
-    67592, 66069, 66324, 65575, 69634, 198411, 197143, 65578, 69890, 67338, 133131, 131608,
-    66327, 65579, 70146, 133130, 66073, 67851, 131864, 65580, 70402, 198922, 197401, 65581,
-    68099, 197641, 196883, 65570, 68355, 66572, 132361, 131350, 66067, 65573, 68611, 66573,
-    132617, 131351, 66323, 65574, 68867, 132364, 65818, 67337, 131606, 65577, 69379, 132621,
-    65820, 67849, 131863, 65579, 69123, 66829, 67084, 65819, 67593, 66071, 66326, 65578,
-    69635, 198412, 197146, 65582, 69891, 67341, 133132, 131611, 66330, 65583, 70147, 133133,
-    66076, 67852, 131867, 65584, 70403, 198925, 197404, 65585, 68100, 197643, 196884, 65571,
-    68356, 66573, 132363, 131351, 66068, 65574, 68612, 66574, 132619, 131352, 66324, 65575,
-    68868, 132365, 65819, 67339, 131607, 65578, 69380, 132622, 65821, 67851, 131864, 65580,
-    69124, 66830, 67085, 65820, 67595, 66072, 66327, 65579, 69636, 198413, 197147, 65583,
-    69892, 67342, 133133, 131612, 66331, 65584, 70148, 133134, 66077, 67853, 131868, 65585,
-    70404, 198926, 197405, 65586, 68101, 197642, 196885, 65572, 68357, 66574, 132362, 131352,
-    66069, 65575, 68613, 66575, 132618, 131353, 66325, 65576, 68869, 132366, 65820, 67338,
-    131608, 65579, 69381, 132623, 65822, 67850, 131865, 65581, 69125, 66831, 67086, 65821,
-    67594, 66073, 66328, 65580, 69637, 198414, 197148, 65584, 69893, 67343, 133134, 131613,
-    66332, 65585, 70149, 133135, 66078, 67854, 131869, 65586, 70405, 198927, 197406, 65587,
-};
-__device__ const uint16_t kKetOff_dffp[31] = {
-    0, 2, 4, 6, 8, 10, 12, 14, 16, 18, 20, 22,
-    24, 26, 28, 30, 32, 34, 36, 38, 40, 42, 44, 46,
-    48, 50, 52, 54, 56, 58, 60,
-};
-__device__ const uint32_t kKetTerm_dffp[60] = {
-    65792, 65546, 66048, 65547, 66304, 65548, 65793, 65547, 66049, 65549, 66305, 65550,
-    65794, 65548, 66050, 65550, 66306, 65551, 65795, 65549, 66051, 65552, 66307, 65553,
-    65796, 65551, 66052, 65554, 66308, 65555, 65797, 65550, 66053, 65553, 66309, 65554,
-    65798, 65552, 66054, 65556, 66310, 65557, 65799, 65553, 66055, 65557, 66311, 65558,
-    65800, 65554, 66056, 65558, 66312, 65559, 65801, 65555, 66057, 65559, 66313, 65560,
-};
 __device__ const double kNormAB_dffp[60] = {
     0.14907119849998599, 0.3333333333333334, 0.3333333333333334, 0.3333333333333334,
     0.3333333333333334, 0.5773502691896258, 0.14907119849998599, 0.3333333333333334,
@@ -199,21 +434,12 @@ __device__ const double kNormAB_dffp[60] = {
     0.3333333333333334, 0.3333333333333334, 0.3333333333333334, 0.5773502691896258,
     0.14907119849998599, 0.3333333333333334, 0.3333333333333334, 0.14907119849998599,
 };
-__device__ const double kNormCD_dffp[30] = {
-    0.2581988897471611, 0.2581988897471611, 0.2581988897471611, 0.5773502691896258,
-    0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
-    0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
-    0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 1.0,
-    1.0, 1.0, 0.2581988897471611, 0.2581988897471611,
-    0.2581988897471611, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
-    0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.2581988897471611,
-    0.2581988897471611, 0.2581988897471611,
-};
 
+// column components cx | cy << 4 | cz << 8
+__device__ const uint16_t kCol_dffp[25] = { 3, 18, 258, 33, 513, 273, 48, 288, 528, 768, 4, 19, 259, 34, 274, 514, 49, 289, 529, 769, 64, 304, 544, 784, 1024 };
 
 __device__ __forceinline__ RysClassTabs tabs_dffp() {
-    return RysClassTabs{kBlk_dffp, kBraOff_dffp, kBraTerm_dffp, kKetOff_dffp, kKetTerm_dffp,
-                        kNormAB_dffp, kNormCD_dffp, nullptr};
+    return RysClassTabs{kNormAB_dffp, kCol_dffp};
 }
 
 template <int MIXED>
@@ -226,8 +452,8 @@ static void rys_prepare_dffp() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_dffp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 47120);
-        cudaFuncSetAttribute(rys_queue_dffp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 47120);
+        cudaFuncSetAttribute(rys_queue_dffp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 107520);
+        cudaFuncSetAttribute(rys_queue_dffp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 107520);
 
         done[dev] = true;
     }
@@ -239,16 +465,16 @@ void launch_rys_dffp(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_dffp();
     constexpr int ng = 128 / C_dffp::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_dffp<1><<<grid, 128, 47120, s>>>(Q, R);
-    else rys_queue_dffp<0><<<grid, 128, 47120, s>>>(Q, R);
+    if (mixed) rys_queue_dffp<1><<<grid, 128, 107520, s>>>(Q, R);
+    else rys_queue_dffp<0><<<grid, 128, 107520, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_dffp(int mixed) {
     rys_prepare_dffp();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dffp<1>, 128, 47120);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dffp<0>, 128, 47120);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dffp<1>, 128, 107520);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dffp<0>, 128, 107520);
     return n;
 }
 

@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (df|ss).  Do not edit.
-// roots 3, block 52 x 1, outputs 60 x 1, group 32 threads,
-// 10 primitive quartets per batch, 1 slot(s), 2 accumulators per thread, 18560 B shared per block.
+// roots 3, block 52 x 1, outputs 60 x 1, group 32 threads, 4 ket pairs a round,
+// 2 primitive quartets per ket pair and batch, 15360 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,67 +11,353 @@ struct C_dfss {
     static constexpr int NA = 52, NC = 1, NBLK = 52;
     static constexpr int NB = 10, ND = 1;
     static constexpr int NAB = 60, NCD = 1;
-    static constexpr int G = 32, NPB = 10, NSLOT = 1, ACC = 2;
-    static constexpr int S = 6;
-    static constexpr int SMEM_GROUP = 580;
-    static constexpr bool COL = false;
+    static constexpr int G = 32, W = 4, H = 8, PB = 2;
+    static constexpr int S = 6, SI = 19, NCP = 1, NCDP = 1;
+    static constexpr int SMEM_GROUP = 480;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
-    __device__ __forceinline__ static void col_update(const T *, const T *, const T *, A *) {}
+    __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
+        acc[0] = fma(x[2] * y[0], z[0], acc[0]);
+        acc[1] = fma(x[1] * y[1], z[0], acc[1]);
+        acc[2] = fma(x[1] * y[0], z[1], acc[2]);
+        acc[3] = fma(x[0] * y[2], z[0], acc[3]);
+        acc[4] = fma(x[0] * y[1], z[1], acc[4]);
+        acc[5] = fma(x[0] * y[0], z[2], acc[5]);
+        acc[6] = fma(x[3] * y[0], z[0], acc[6]);
+        acc[7] = fma(x[2] * y[1], z[0], acc[7]);
+        acc[8] = fma(x[2] * y[0], z[1], acc[8]);
+        acc[9] = fma(x[1] * y[2], z[0], acc[9]);
+        acc[10] = fma(x[1] * y[0], z[2], acc[10]);
+        acc[11] = fma(x[1] * y[1], z[1], acc[11]);
+        acc[12] = fma(x[0] * y[3], z[0], acc[12]);
+        acc[13] = fma(x[0] * y[2], z[1], acc[13]);
+        acc[14] = fma(x[0] * y[1], z[2], acc[14]);
+        acc[15] = fma(x[0] * y[0], z[3], acc[15]);
+        acc[16] = fma(x[4] * y[0], z[0], acc[16]);
+        acc[17] = fma(x[3] * y[1], z[0], acc[17]);
+        acc[18] = fma(x[3] * y[0], z[1], acc[18]);
+        acc[19] = fma(x[2] * y[2], z[0], acc[19]);
+        acc[20] = fma(x[2] * y[1], z[1], acc[20]);
+        acc[21] = fma(x[2] * y[0], z[2], acc[21]);
+        acc[22] = fma(x[1] * y[3], z[0], acc[22]);
+        acc[23] = fma(x[1] * y[2], z[1], acc[23]);
+        acc[24] = fma(x[1] * y[1], z[2], acc[24]);
+        acc[25] = fma(x[1] * y[0], z[3], acc[25]);
+        acc[26] = fma(x[0] * y[4], z[0], acc[26]);
+        acc[27] = fma(x[0] * y[3], z[1], acc[27]);
+        acc[28] = fma(x[0] * y[2], z[2], acc[28]);
+        acc[29] = fma(x[0] * y[1], z[3], acc[29]);
+        acc[30] = fma(x[0] * y[0], z[4], acc[30]);
+        acc[31] = fma(x[5] * y[0], z[0], acc[31]);
+        acc[32] = fma(x[4] * y[1], z[0], acc[32]);
+        acc[33] = fma(x[4] * y[0], z[1], acc[33]);
+        acc[34] = fma(x[3] * y[2], z[0], acc[34]);
+        acc[35] = fma(x[3] * y[1], z[1], acc[35]);
+        acc[36] = fma(x[3] * y[0], z[2], acc[36]);
+        acc[37] = fma(x[2] * y[3], z[0], acc[37]);
+        acc[38] = fma(x[2] * y[2], z[1], acc[38]);
+        acc[39] = fma(x[2] * y[1], z[2], acc[39]);
+        acc[40] = fma(x[2] * y[0], z[3], acc[40]);
+        acc[41] = fma(x[1] * y[4], z[0], acc[41]);
+        acc[42] = fma(x[1] * y[3], z[1], acc[42]);
+        acc[43] = fma(x[1] * y[2], z[2], acc[43]);
+        acc[44] = fma(x[1] * y[1], z[3], acc[44]);
+        acc[45] = fma(x[1] * y[0], z[4], acc[45]);
+        acc[46] = fma(x[0] * y[5], z[0], acc[46]);
+        acc[47] = fma(x[0] * y[4], z[1], acc[47]);
+        acc[48] = fma(x[0] * y[3], z[2], acc[48]);
+        acc[49] = fma(x[0] * y[2], z[3], acc[49]);
+        acc[50] = fma(x[0] * y[1], z[4], acc[50]);
+        acc[51] = fma(x[0] * y[0], z[5], acc[51]);
+    }
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[16], in[31]);
+        const double h1 = fma(x, in[6], in[16]);
+        const double h2 = fma(x, h1, h0);
+        const double h3 = fma(x, in[0], in[6]);
+        const double h4 = fma(x, h3, h1);
+        const double h5 = fma(x, h4, h2);
+        const double h6 = fma(y, in[16], in[32]);
+        const double h7 = fma(y, in[6], in[17]);
+        const double h8 = fma(x, h7, h6);
+        const double h9 = fma(y, in[0], in[7]);
+        const double h10 = fma(x, h9, h7);
+        const double h11 = fma(x, h10, h8);
+        const double h12 = fma(z, in[16], in[33]);
+        const double h13 = fma(z, in[6], in[18]);
+        const double h14 = fma(x, h13, h12);
+        const double h15 = fma(z, in[0], in[8]);
+        const double h16 = fma(x, h15, h13);
+        const double h17 = fma(x, h16, h14);
+        const double h18 = fma(y, in[17], in[34]);
+        const double h19 = fma(y, in[7], in[19]);
+        const double h20 = fma(x, h19, h18);
+        const double h21 = fma(y, h10, h20);
+        const double h22 = fma(z, in[18], in[36]);
+        const double h23 = fma(z, in[8], in[21]);
+        const double h24 = fma(x, h23, h22);
+        const double h25 = fma(z, h16, h24);
+        const double h26 = fma(z, in[17], in[35]);
+        const double h27 = fma(y, h13, h26);
+        const double h28 = fma(z, in[7], in[20]);
+        const double h29 = fma(y, h15, h28);
+        const double h30 = fma(x, h29, h27);
+        const double h31 = fma(y, in[19], in[37]);
+        const double h32 = fma(y, h19, h31);
+        const double h33 = fma(y, h9, h19);
+        const double h34 = fma(y, h33, h32);
+        const double h35 = fma(z, in[19], in[38]);
+        const double h36 = fma(y, h28, h35);
+        const double h37 = fma(y, h29, h36);
+        const double h38 = fma(z, in[20], in[39]);
+        const double h39 = fma(y, h23, h38);
+        const double h40 = fma(z, h29, h39);
+        const double h41 = fma(z, in[21], in[40]);
+        const double h42 = fma(z, h23, h41);
+        const double h43 = fma(z, h15, h23);
+        const double h44 = fma(z, h43, h42);
+        const double h45 = fma(x, in[17], in[32]);
+        const double h46 = fma(x, in[7], in[17]);
+        const double h47 = fma(x, h46, h45);
+        const double h48 = fma(x, in[1], in[7]);
+        const double h49 = fma(x, h48, h46);
+        const double h50 = fma(x, h49, h47);
+        const double h51 = fma(y, in[1], in[9]);
+        const double h52 = fma(x, h51, h19);
+        const double h53 = fma(x, h52, h20);
+        const double h54 = fma(x, h28, h26);
+        const double h55 = fma(z, in[1], in[11]);
+        const double h56 = fma(x, h55, h28);
+        const double h57 = fma(x, h56, h54);
+        const double h58 = fma(y, in[9], in[22]);
+        const double h59 = fma(x, h58, h31);
+        const double h60 = fma(y, h52, h59);
+        const double h61 = fma(z, in[11], in[24]);
+        const double h62 = fma(x, h61, h38);
+        const double h63 = fma(z, h56, h62);
+        const double h64 = fma(z, in[9], in[23]);
+        const double h65 = fma(y, h55, h64);
+        const double h66 = fma(x, h65, h36);
+        const double h67 = fma(y, in[22], in[41]);
+        const double h68 = fma(y, h58, h67);
+        const double h69 = fma(y, h51, h58);
+        const double h70 = fma(y, h69, h68);
+        const double h71 = fma(z, in[22], in[42]);
+        const double h72 = fma(y, h64, h71);
+        const double h73 = fma(y, h65, h72);
+        const double h74 = fma(z, in[23], in[43]);
+        const double h75 = fma(y, h61, h74);
+        const double h76 = fma(z, h65, h75);
+        const double h77 = fma(z, in[24], in[44]);
+        const double h78 = fma(z, h61, h77);
+        const double h79 = fma(z, h55, h61);
+        const double h80 = fma(z, h79, h78);
+        const double h81 = fma(x, in[18], in[33]);
+        const double h82 = fma(x, in[8], in[18]);
+        const double h83 = fma(x, h82, h81);
+        const double h84 = fma(x, in[2], in[8]);
+        const double h85 = fma(x, h84, h82);
+        const double h86 = fma(x, h85, h83);
+        const double h87 = fma(y, in[18], in[35]);
+        const double h88 = fma(y, in[8], in[20]);
+        const double h89 = fma(x, h88, h87);
+        const double h90 = fma(y, in[2], in[11]);
+        const double h91 = fma(x, h90, h88);
+        const double h92 = fma(x, h91, h89);
+        const double h93 = fma(z, in[2], in[10]);
+        const double h94 = fma(x, h93, h23);
+        const double h95 = fma(x, h94, h24);
+        const double h96 = fma(y, in[20], in[38]);
+        const double h97 = fma(y, in[11], in[23]);
+        const double h98 = fma(x, h97, h96);
+        const double h99 = fma(y, h91, h98);
+        const double h100 = fma(z, in[10], in[25]);
+        const double h101 = fma(x, h100, h41);
+        const double h102 = fma(z, h94, h101);
+        const double h103 = fma(y, h93, h61);
+        const double h104 = fma(x, h103, h39);
+        const double h105 = fma(y, in[23], in[42]);
+        const double h106 = fma(y, h97, h105);
+        const double h107 = fma(y, h90, h97);
+        const double h108 = fma(y, h107, h106);
+        const double h109 = fma(y, h103, h75);
+        const double h110 = fma(y, h100, h77);
+        const double h111 = fma(z, h103, h110);
+        const double h112 = fma(z, in[25], in[45]);
+        const double h113 = fma(z, h100, h112);
+        const double h114 = fma(z, h93, h100);
+        const double h115 = fma(z, h114, h113);
+        const double h116 = fma(x, in[19], in[34]);
+        const double h117 = fma(x, in[9], in[19]);
+        const double h118 = fma(x, h117, h116);
+        const double h119 = fma(x, in[3], in[9]);
+        const double h120 = fma(x, h119, h117);
+        const double h121 = fma(x, h120, h118);
+        const double h122 = fma(y, in[3], in[12]);
+        const double h123 = fma(x, h122, h58);
+        const double h124 = fma(x, h123, h59);
+        const double h125 = fma(x, h64, h35);
+        const double h126 = fma(z, in[3], in[13]);
+        const double h127 = fma(x, h126, h64);
+        const double h128 = fma(x, h127, h125);
+        const double h129 = fma(y, in[12], in[26]);
+        const double h130 = fma(x, h129, h67);
+        const double h131 = fma(y, h123, h130);
+        const double h132 = fma(z, in[13], in[28]);
+        const double h133 = fma(x, h132, h74);
+        const double h134 = fma(z, h127, h133);
+        const double h135 = fma(z, in[12], in[27]);
+        const double h136 = fma(y, h126, h135);
+        const double h137 = fma(x, h136, h72);
+        const double h138 = fma(y, in[26], in[46]);
+        const double h139 = fma(y, h129, h138);
+        const double h140 = fma(y, h122, h129);
+        const double h141 = fma(y, h140, h139);
+        const double h142 = fma(z, in[26], in[47]);
+        const double h143 = fma(y, h135, h142);
+        const double h144 = fma(y, h136, h143);
+        const double h145 = fma(z, in[27], in[48]);
+        const double h146 = fma(y, h132, h145);
+        const double h147 = fma(z, h136, h146);
+        const double h148 = fma(z, in[28], in[49]);
+        const double h149 = fma(z, h132, h148);
+        const double h150 = fma(z, h126, h132);
+        const double h151 = fma(z, h150, h149);
+        const double h152 = fma(x, in[20], in[35]);
+        const double h153 = fma(x, in[11], in[20]);
+        const double h154 = fma(x, h153, h152);
+        const double h155 = fma(x, in[4], in[11]);
+        const double h156 = fma(x, h155, h153);
+        const double h157 = fma(x, h156, h154);
+        const double h158 = fma(y, in[4], in[13]);
+        const double h159 = fma(x, h158, h97);
+        const double h160 = fma(x, h159, h98);
+        const double h161 = fma(z, in[4], in[14]);
+        const double h162 = fma(x, h161, h61);
+        const double h163 = fma(x, h162, h62);
+        const double h164 = fma(y, in[13], in[27]);
+        const double h165 = fma(x, h164, h105);
+        const double h166 = fma(y, h159, h165);
+        const double h167 = fma(z, in[14], in[29]);
+        const double h168 = fma(x, h167, h77);
+        const double h169 = fma(z, h162, h168);
+        const double h170 = fma(y, h161, h132);
+        const double h171 = fma(x, h170, h75);
+        const double h172 = fma(y, in[27], in[47]);
+        const double h173 = fma(y, h164, h172);
+        const double h174 = fma(y, h158, h164);
+        const double h175 = fma(y, h174, h173);
+        const double h176 = fma(y, h170, h146);
+        const double h177 = fma(y, h167, h148);
+        const double h178 = fma(z, h170, h177);
+        const double h179 = fma(z, in[29], in[50]);
+        const double h180 = fma(z, h167, h179);
+        const double h181 = fma(z, h161, h167);
+        const double h182 = fma(z, h181, h180);
+        const double h183 = fma(x, in[21], in[36]);
+        const double h184 = fma(x, in[10], in[21]);
+        const double h185 = fma(x, h184, h183);
+        const double h186 = fma(x, in[5], in[10]);
+        const double h187 = fma(x, h186, h184);
+        const double h188 = fma(x, h187, h185);
+        const double h189 = fma(y, in[21], in[39]);
+        const double h190 = fma(y, in[10], in[24]);
+        const double h191 = fma(x, h190, h189);
+        const double h192 = fma(y, in[5], in[14]);
+        const double h193 = fma(x, h192, h190);
+        const double h194 = fma(x, h193, h191);
+        const double h195 = fma(z, in[5], in[15]);
+        const double h196 = fma(x, h195, h100);
+        const double h197 = fma(x, h196, h101);
+        const double h198 = fma(y, in[24], in[43]);
+        const double h199 = fma(y, in[14], in[28]);
+        const double h200 = fma(x, h199, h198);
+        const double h201 = fma(y, h193, h200);
+        const double h202 = fma(z, in[15], in[30]);
+        const double h203 = fma(x, h202, h112);
+        const double h204 = fma(z, h196, h203);
+        const double h205 = fma(y, h195, h167);
+        const double h206 = fma(x, h205, h110);
+        const double h207 = fma(y, in[28], in[48]);
+        const double h208 = fma(y, h199, h207);
+        const double h209 = fma(y, h192, h199);
+        const double h210 = fma(y, h209, h208);
+        const double h211 = fma(y, h205, h177);
+        const double h212 = fma(y, h202, h179);
+        const double h213 = fma(z, h205, h212);
+        const double h214 = fma(z, in[30], in[51]);
+        const double h215 = fma(z, h202, h214);
+        const double h216 = fma(z, h195, h202);
+        const double h217 = fma(z, h216, h215);
+        out[0] = h5;
+        out[1] = h11;
+        out[2] = h17;
+        out[3] = h21;
+        out[4] = h25;
+        out[5] = h30;
+        out[6] = h34;
+        out[7] = h37;
+        out[8] = h40;
+        out[9] = h44;
+        out[10] = h50;
+        out[11] = h53;
+        out[12] = h57;
+        out[13] = h60;
+        out[14] = h63;
+        out[15] = h66;
+        out[16] = h70;
+        out[17] = h73;
+        out[18] = h76;
+        out[19] = h80;
+        out[20] = h86;
+        out[21] = h92;
+        out[22] = h95;
+        out[23] = h99;
+        out[24] = h102;
+        out[25] = h104;
+        out[26] = h108;
+        out[27] = h109;
+        out[28] = h111;
+        out[29] = h115;
+        out[30] = h121;
+        out[31] = h124;
+        out[32] = h128;
+        out[33] = h131;
+        out[34] = h134;
+        out[35] = h137;
+        out[36] = h141;
+        out[37] = h144;
+        out[38] = h147;
+        out[39] = h151;
+        out[40] = h157;
+        out[41] = h160;
+        out[42] = h163;
+        out[43] = h166;
+        out[44] = h169;
+        out[45] = h171;
+        out[46] = h175;
+        out[47] = h176;
+        out[48] = h178;
+        out[49] = h182;
+        out[50] = h188;
+        out[51] = h194;
+        out[52] = h197;
+        out[53] = h201;
+        out[54] = h204;
+        out[55] = h206;
+        out[56] = h210;
+        out[57] = h211;
+        out[58] = h213;
+        out[59] = h217;
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        out[0] = in[0] * (nrm * 1.0);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_dfss[52] = {
-    2, 257, 65537, 512, 65792, 131072, 3, 258, 65538, 513, 131073, 65793,
-    768, 66048, 131328, 196608, 4, 259, 65539, 514, 65794, 131074, 769, 66049,
-    131329, 196609, 1024, 66304, 131584, 196864, 262144, 5, 260, 65540, 515, 65795,
-    131075, 770, 66050, 131330, 196610, 1025, 66305, 131585, 196865, 262145, 1280, 66560,
-    131840, 197120, 262400, 327680,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_dfss[61] = {
-    0, 4, 10, 16, 22, 28, 36, 40, 46, 52, 56, 60,
-    66, 72, 78, 84, 92, 96, 102, 108, 112, 116, 122, 128,
-    134, 140, 148, 152, 158, 164, 168, 172, 178, 184, 190, 196,
-    204, 208, 214, 220, 224, 228, 234, 240, 246, 252, 260, 264,
-    270, 276, 280, 284, 290, 296, 302, 308, 316, 320, 326, 332,
-    336,
-};
-__device__ const uint32_t kBraTerm_dfss[336] = {
-    68096, 197638, 196880, 65567, 68352, 66567, 132358, 131345, 66064, 65568, 68608, 66568,
-    132614, 131346, 66320, 65569, 68864, 132359, 65811, 67334, 131601, 65570, 69376, 132616,
-    65813, 67846, 131858, 65572, 69120, 66824, 67079, 65812, 67590, 66066, 66321, 65571,
-    69632, 198407, 197139, 65573, 69888, 67336, 133127, 131604, 66323, 65574, 70144, 133128,
-    66069, 67847, 131860, 65575, 70400, 198920, 197397, 65576, 68097, 197639, 196881, 65568,
-    68353, 66569, 132359, 131347, 66065, 65570, 68609, 66571, 132615, 131348, 66321, 65571,
-    68865, 132361, 65814, 67335, 131603, 65573, 69377, 132619, 65816, 67847, 131860, 65575,
-    69121, 66827, 67081, 65815, 67591, 66068, 66323, 65574, 69633, 198409, 197142, 65577,
-    69889, 67339, 133129, 131607, 66326, 65578, 70145, 133131, 66072, 67849, 131863, 65579,
-    70401, 198923, 197400, 65580, 68098, 197640, 196882, 65569, 68354, 66571, 132360, 131348,
-    66066, 65571, 68610, 66570, 132616, 131349, 66322, 65572, 68866, 132363, 65815, 67336,
-    131604, 65574, 69378, 132618, 65817, 67848, 131861, 65576, 69122, 66826, 67083, 65816,
-    67592, 66069, 66324, 65575, 69634, 198411, 197143, 65578, 69890, 67338, 133131, 131608,
-    66327, 65579, 70146, 133130, 66073, 67851, 131864, 65580, 70402, 198922, 197401, 65581,
-    68099, 197641, 196883, 65570, 68355, 66572, 132361, 131350, 66067, 65573, 68611, 66573,
-    132617, 131351, 66323, 65574, 68867, 132364, 65818, 67337, 131606, 65577, 69379, 132621,
-    65820, 67849, 131863, 65579, 69123, 66829, 67084, 65819, 67593, 66071, 66326, 65578,
-    69635, 198412, 197146, 65582, 69891, 67341, 133132, 131611, 66330, 65583, 70147, 133133,
-    66076, 67852, 131867, 65584, 70403, 198925, 197404, 65585, 68100, 197643, 196884, 65571,
-    68356, 66573, 132363, 131351, 66068, 65574, 68612, 66574, 132619, 131352, 66324, 65575,
-    68868, 132365, 65819, 67339, 131607, 65578, 69380, 132622, 65821, 67851, 131864, 65580,
-    69124, 66830, 67085, 65820, 67595, 66072, 66327, 65579, 69636, 198413, 197147, 65583,
-    69892, 67342, 133133, 131612, 66331, 65584, 70148, 133134, 66077, 67853, 131868, 65585,
-    70404, 198926, 197405, 65586, 68101, 197642, 196885, 65572, 68357, 66574, 132362, 131352,
-    66069, 65575, 68613, 66575, 132618, 131353, 66325, 65576, 68869, 132366, 65820, 67338,
-    131608, 65579, 69381, 132623, 65822, 67850, 131865, 65581, 69125, 66831, 67086, 65821,
-    67594, 66073, 66328, 65580, 69637, 198414, 197148, 65584, 69893, 67343, 133134, 131613,
-    66332, 65585, 70149, 133135, 66078, 67854, 131869, 65586, 70405, 198927, 197406, 65587,
-};
-__device__ const uint16_t kKetOff_dfss[2] = {
-    0, 1,
-};
-__device__ const uint32_t kKetTerm_dfss[1] = {
-    65536,
-};
 __device__ const double kNormAB_dfss[60] = {
     0.14907119849998599, 0.3333333333333334, 0.3333333333333334, 0.3333333333333334,
     0.3333333333333334, 0.5773502691896258, 0.14907119849998599, 0.3333333333333334,
@@ -89,14 +375,12 @@ __device__ const double kNormAB_dfss[60] = {
     0.3333333333333334, 0.3333333333333334, 0.3333333333333334, 0.5773502691896258,
     0.14907119849998599, 0.3333333333333334, 0.3333333333333334, 0.14907119849998599,
 };
-__device__ const double kNormCD_dfss[1] = {
-    1.0,
-};
 
+// column components cx | cy << 4 | cz << 8
+__device__ const uint16_t kCol_dfss[1] = { 0 };
 
 __device__ __forceinline__ RysClassTabs tabs_dfss() {
-    return RysClassTabs{kBlk_dfss, kBraOff_dfss, kBraTerm_dfss, kKetOff_dfss, kKetTerm_dfss,
-                        kNormAB_dfss, kNormCD_dfss, nullptr};
+    return RysClassTabs{kNormAB_dfss, kCol_dfss};
 }
 
 template <int MIXED>
@@ -109,8 +393,8 @@ static void rys_prepare_dfss() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_dfss<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 18560);
-        cudaFuncSetAttribute(rys_queue_dfss<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 18560);
+        cudaFuncSetAttribute(rys_queue_dfss<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 15360);
+        cudaFuncSetAttribute(rys_queue_dfss<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 15360);
 
         done[dev] = true;
     }
@@ -122,16 +406,16 @@ void launch_rys_dfss(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_dfss();
     constexpr int ng = 128 / C_dfss::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_dfss<1><<<grid, 128, 18560, s>>>(Q, R);
-    else rys_queue_dfss<0><<<grid, 128, 18560, s>>>(Q, R);
+    if (mixed) rys_queue_dfss<1><<<grid, 128, 15360, s>>>(Q, R);
+    else rys_queue_dfss<0><<<grid, 128, 15360, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_dfss(int mixed) {
     rys_prepare_dfss();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dfss<1>, 128, 18560);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dfss<0>, 128, 18560);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dfss<1>, 128, 15360);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dfss<0>, 128, 15360);
     return n;
 }
 

@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (dp|pp).  Do not edit.
-// roots 3, block 16 x 9, outputs 18 x 9, group 64 threads,
-// 21 primitive quartets per batch, 1 slot(s), 3 accumulators per thread, 36928 B shared per block.
+// roots 3, block 16 x 9, outputs 18 x 9, group 32 threads, 3 ket pairs a round,
+// 3 primitive quartets per ket pair and batch, 31968 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,46 +11,92 @@ struct C_dppp {
     static constexpr int NA = 16, NC = 9, NBLK = 144;
     static constexpr int NB = 3, ND = 3;
     static constexpr int NAB = 18, NCD = 9;
-    static constexpr int G = 64, NPB = 21, NSLOT = 1, ACC = 3;
-    static constexpr int S = 12;
-    static constexpr int SMEM_GROUP = 2308;
-    static constexpr bool COL = false;
+    static constexpr int G = 32, W = 3, H = 1, PB = 3;
+    static constexpr int S = 12, SI = 37, NCP = 9, NCDP = 9;
+    static constexpr int SMEM_GROUP = 999;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
-    __device__ __forceinline__ static void col_update(const T *, const T *, const T *, A *) {}
+    __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
+        acc[0] = fma(x[2] * y[0], z[0], acc[0]);
+        acc[1] = fma(x[1] * y[1], z[0], acc[1]);
+        acc[2] = fma(x[1] * y[0], z[1], acc[2]);
+        acc[3] = fma(x[0] * y[2], z[0], acc[3]);
+        acc[4] = fma(x[0] * y[1], z[1], acc[4]);
+        acc[5] = fma(x[0] * y[0], z[2], acc[5]);
+        acc[6] = fma(x[3] * y[0], z[0], acc[6]);
+        acc[7] = fma(x[2] * y[1], z[0], acc[7]);
+        acc[8] = fma(x[2] * y[0], z[1], acc[8]);
+        acc[9] = fma(x[1] * y[2], z[0], acc[9]);
+        acc[10] = fma(x[1] * y[0], z[2], acc[10]);
+        acc[11] = fma(x[1] * y[1], z[1], acc[11]);
+        acc[12] = fma(x[0] * y[3], z[0], acc[12]);
+        acc[13] = fma(x[0] * y[2], z[1], acc[13]);
+        acc[14] = fma(x[0] * y[1], z[2], acc[14]);
+        acc[15] = fma(x[0] * y[0], z[3], acc[15]);
+    }
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[0], in[6]);
+        const double h1 = fma(y, in[0], in[7]);
+        const double h2 = fma(z, in[0], in[8]);
+        const double h3 = fma(x, in[1], in[7]);
+        const double h4 = fma(y, in[1], in[9]);
+        const double h5 = fma(z, in[1], in[11]);
+        const double h6 = fma(x, in[2], in[8]);
+        const double h7 = fma(y, in[2], in[11]);
+        const double h8 = fma(z, in[2], in[10]);
+        const double h9 = fma(x, in[3], in[9]);
+        const double h10 = fma(y, in[3], in[12]);
+        const double h11 = fma(z, in[3], in[13]);
+        const double h12 = fma(x, in[4], in[11]);
+        const double h13 = fma(y, in[4], in[13]);
+        const double h14 = fma(z, in[4], in[14]);
+        const double h15 = fma(x, in[5], in[10]);
+        const double h16 = fma(y, in[5], in[14]);
+        const double h17 = fma(z, in[5], in[15]);
+        out[0] = h0;
+        out[9] = h1;
+        out[18] = h2;
+        out[27] = h3;
+        out[36] = h4;
+        out[45] = h5;
+        out[54] = h6;
+        out[63] = h7;
+        out[72] = h8;
+        out[81] = h9;
+        out[90] = h10;
+        out[99] = h11;
+        out[108] = h12;
+        out[117] = h13;
+        out[126] = h14;
+        out[135] = h15;
+        out[144] = h16;
+        out[153] = h17;
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[0], in[3]);
+        const double h1 = fma(y, in[0], in[4]);
+        const double h2 = fma(z, in[0], in[5]);
+        const double h3 = fma(x, in[1], in[4]);
+        const double h4 = fma(y, in[1], in[6]);
+        const double h5 = fma(z, in[1], in[7]);
+        const double h6 = fma(x, in[2], in[5]);
+        const double h7 = fma(y, in[2], in[7]);
+        const double h8 = fma(z, in[2], in[8]);
+        out[0] = h0 * (nrm * 1.0);
+        out[1] = h1 * (nrm * 1.0);
+        out[2] = h2 * (nrm * 1.0);
+        out[3] = h3 * (nrm * 1.0);
+        out[4] = h4 * (nrm * 1.0);
+        out[5] = h5 * (nrm * 1.0);
+        out[6] = h6 * (nrm * 1.0);
+        out[7] = h7 * (nrm * 1.0);
+        out[8] = h8 * (nrm * 1.0);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_dppp[144] = {
-    7, 262, 65542, 8, 263, 65543, 518, 65798, 131078, 772, 1027, 66307,
-    773, 1028, 66308, 1283, 66563, 131843, 196612, 196867, 262147, 196613, 196868, 262148,
-    197123, 262403, 327683, 1537, 1792, 67072, 1538, 1793, 67073, 2048, 67328, 132608,
-    197377, 197632, 262912, 197378, 197633, 262913, 197888, 263168, 328448, 393217, 393472, 458752,
-    393218, 393473, 458753, 393728, 459008, 524288, 10, 265, 65545, 11, 266, 65546,
-    521, 65801, 131081, 775, 1030, 66310, 776, 1031, 66311, 1286, 66566, 131846,
-    196615, 196870, 262150, 196616, 196871, 262151, 197126, 262406, 327686, 1540, 1795, 67075,
-    1541, 1796, 67076, 2051, 67331, 132611, 393220, 393475, 458755, 393221, 393476, 458756,
-    393731, 459011, 524291, 197380, 197635, 262915, 197381, 197636, 262916, 197891, 263171, 328451,
-    2305, 2560, 67840, 2306, 2561, 67841, 2816, 68096, 133376, 198145, 198400, 263680,
-    198146, 198401, 263681, 198656, 263936, 329216, 393985, 394240, 459520, 393986, 394241, 459521,
-    394496, 459776, 525056, 589825, 590080, 655360, 589826, 590081, 655361, 590336, 655616, 720896,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_dppp[19] = {
-    0, 2, 4, 6, 8, 10, 12, 14, 16, 18, 20, 22,
-    24, 26, 28, 30, 32, 34, 36,
-};
-__device__ const uint32_t kBraTerm_dppp[36] = {
-    65792, 65542, 66048, 65543, 66304, 65544, 65793, 65543, 66049, 65545, 66305, 65547,
-    65794, 65544, 66050, 65547, 66306, 65546, 65795, 65545, 66051, 65548, 66307, 65549,
-    65796, 65547, 66052, 65549, 66308, 65550, 65797, 65546, 66053, 65550, 66309, 65551,
-};
-__device__ const uint16_t kKetOff_dppp[10] = {
-    0, 2, 4, 6, 8, 10, 12, 14, 16, 18,
-};
-__device__ const uint32_t kKetTerm_dppp[18] = {
-    65792, 65539, 66048, 65540, 66304, 65541, 65793, 65540, 66049, 65542, 66305, 65543,
-    65794, 65541, 66050, 65543, 66306, 65544,
-};
 __device__ const double kNormAB_dppp[18] = {
     0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 1.0,
     1.0, 1.0, 1.0, 1.0,
@@ -58,16 +104,12 @@ __device__ const double kNormAB_dppp[18] = {
     1.0, 1.0, 1.0, 0.5773502691896258,
     0.5773502691896258, 0.5773502691896258,
 };
-__device__ const double kNormCD_dppp[9] = {
-    1.0, 1.0, 1.0, 1.0,
-    1.0, 1.0, 1.0, 1.0,
-    1.0,
-};
 
+// column components cx | cy << 4 | cz << 8
+__device__ const uint16_t kCol_dppp[9] = { 1, 16, 256, 2, 17, 257, 32, 272, 512 };
 
 __device__ __forceinline__ RysClassTabs tabs_dppp() {
-    return RysClassTabs{kBlk_dppp, kBraOff_dppp, kBraTerm_dppp, kKetOff_dppp, kKetTerm_dppp,
-                        kNormAB_dppp, kNormCD_dppp, nullptr};
+    return RysClassTabs{kNormAB_dppp, kCol_dppp};
 }
 
 template <int MIXED>
@@ -80,8 +122,8 @@ static void rys_prepare_dppp() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_dppp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 36928);
-        cudaFuncSetAttribute(rys_queue_dppp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 36928);
+        cudaFuncSetAttribute(rys_queue_dppp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 31968);
+        cudaFuncSetAttribute(rys_queue_dppp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 31968);
 
         done[dev] = true;
     }
@@ -93,16 +135,16 @@ void launch_rys_dppp(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_dppp();
     constexpr int ng = 128 / C_dppp::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_dppp<1><<<grid, 128, 36928, s>>>(Q, R);
-    else rys_queue_dppp<0><<<grid, 128, 36928, s>>>(Q, R);
+    if (mixed) rys_queue_dppp<1><<<grid, 128, 31968, s>>>(Q, R);
+    else rys_queue_dppp<0><<<grid, 128, 31968, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_dppp(int mixed) {
     rys_prepare_dppp();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dppp<1>, 128, 36928);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dppp<0>, 128, 36928);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dppp<1>, 128, 31968);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dppp<0>, 128, 31968);
     return n;
 }
 

@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (ds|pp).  Do not edit.
-// roots 3, block 6 x 9, outputs 6 x 9, group 32 threads,
-// 10 primitive quartets per batch, 1 slot(s), 2 accumulators per thread, 27200 B shared per block.
+// roots 3, block 6 x 9, outputs 6 x 9, group 32 threads, 3 ket pairs a round,
+// 3 primitive quartets per ket pair and batch, 23328 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,50 +11,62 @@ struct C_dspp {
     static constexpr int NA = 6, NC = 9, NBLK = 54;
     static constexpr int NB = 1, ND = 3;
     static constexpr int NAB = 6, NCD = 9;
-    static constexpr int G = 32, NPB = 10, NSLOT = 1, ACC = 2;
-    static constexpr int S = 9;
-    static constexpr int SMEM_GROUP = 850;
-    static constexpr bool COL = false;
+    static constexpr int G = 32, W = 3, H = 1, PB = 3;
+    static constexpr int S = 9, SI = 27, NCP = 9, NCDP = 9;
+    static constexpr int SMEM_GROUP = 729;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
-    __device__ __forceinline__ static void col_update(const T *, const T *, const T *, A *) {}
+    __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
+        acc[0] = fma(x[2] * y[0], z[0], acc[0]);
+        acc[1] = fma(x[1] * y[1], z[0], acc[1]);
+        acc[2] = fma(x[1] * y[0], z[1], acc[2]);
+        acc[3] = fma(x[0] * y[2], z[0], acc[3]);
+        acc[4] = fma(x[0] * y[1], z[1], acc[4]);
+        acc[5] = fma(x[0] * y[0], z[2], acc[5]);
+    }
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        out[0] = in[0];
+        out[9] = in[1];
+        out[18] = in[2];
+        out[27] = in[3];
+        out[36] = in[4];
+        out[45] = in[5];
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[0], in[3]);
+        const double h1 = fma(y, in[0], in[4]);
+        const double h2 = fma(z, in[0], in[5]);
+        const double h3 = fma(x, in[1], in[4]);
+        const double h4 = fma(y, in[1], in[6]);
+        const double h5 = fma(z, in[1], in[7]);
+        const double h6 = fma(x, in[2], in[5]);
+        const double h7 = fma(y, in[2], in[7]);
+        const double h8 = fma(z, in[2], in[8]);
+        out[0] = h0 * (nrm * 1.0);
+        out[1] = h1 * (nrm * 1.0);
+        out[2] = h2 * (nrm * 1.0);
+        out[3] = h3 * (nrm * 1.0);
+        out[4] = h4 * (nrm * 1.0);
+        out[5] = h5 * (nrm * 1.0);
+        out[6] = h6 * (nrm * 1.0);
+        out[7] = h7 * (nrm * 1.0);
+        out[8] = h8 * (nrm * 1.0);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_dspp[54] = {
-    7, 262, 65542, 8, 263, 65543, 518, 65798, 131078, 772, 1027, 66307,
-    773, 1028, 66308, 1283, 66563, 131843, 196612, 196867, 262147, 196613, 196868, 262148,
-    197123, 262403, 327683, 1537, 1792, 67072, 1538, 1793, 67073, 2048, 67328, 132608,
-    197377, 197632, 262912, 197378, 197633, 262913, 197888, 263168, 328448, 393217, 393472, 458752,
-    393218, 393473, 458753, 393728, 459008, 524288,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_dspp[7] = {
-    0, 1, 2, 3, 4, 5, 6,
-};
-__device__ const uint32_t kBraTerm_dspp[6] = {
-    65536, 65537, 65538, 65539, 65540, 65541,
-};
-__device__ const uint16_t kKetOff_dspp[10] = {
-    0, 2, 4, 6, 8, 10, 12, 14, 16, 18,
-};
-__device__ const uint32_t kKetTerm_dspp[18] = {
-    65792, 65539, 66048, 65540, 66304, 65541, 65793, 65540, 66049, 65542, 66305, 65543,
-    65794, 65541, 66050, 65543, 66306, 65544,
-};
 __device__ const double kNormAB_dspp[6] = {
     0.5773502691896258, 1.0, 1.0, 0.5773502691896258,
     1.0, 0.5773502691896258,
 };
-__device__ const double kNormCD_dspp[9] = {
-    1.0, 1.0, 1.0, 1.0,
-    1.0, 1.0, 1.0, 1.0,
-    1.0,
-};
 
+// column components cx | cy << 4 | cz << 8
+__device__ const uint16_t kCol_dspp[9] = { 1, 16, 256, 2, 17, 257, 32, 272, 512 };
 
 __device__ __forceinline__ RysClassTabs tabs_dspp() {
-    return RysClassTabs{kBlk_dspp, kBraOff_dspp, kBraTerm_dspp, kKetOff_dspp, kKetTerm_dspp,
-                        kNormAB_dspp, kNormCD_dspp, nullptr};
+    return RysClassTabs{kNormAB_dspp, kCol_dspp};
 }
 
 template <int MIXED>
@@ -67,8 +79,8 @@ static void rys_prepare_dspp() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_dspp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 27200);
-        cudaFuncSetAttribute(rys_queue_dspp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 27200);
+        cudaFuncSetAttribute(rys_queue_dspp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 23328);
+        cudaFuncSetAttribute(rys_queue_dspp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 23328);
 
         done[dev] = true;
     }
@@ -80,16 +92,16 @@ void launch_rys_dspp(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_dspp();
     constexpr int ng = 128 / C_dspp::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_dspp<1><<<grid, 128, 27200, s>>>(Q, R);
-    else rys_queue_dspp<0><<<grid, 128, 27200, s>>>(Q, R);
+    if (mixed) rys_queue_dspp<1><<<grid, 128, 23328, s>>>(Q, R);
+    else rys_queue_dspp<0><<<grid, 128, 23328, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_dspp(int mixed) {
     rys_prepare_dspp();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dspp<1>, 128, 27200);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dspp<0>, 128, 27200);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dspp<1>, 128, 23328);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dspp<0>, 128, 23328);
     return n;
 }
 

@@ -1,88 +1,211 @@
 // Generated by gen_rys.py -- Rys class (ds|ss).  Do not edit.
-// roots 2, block 6 x 1, outputs 6 x 1, group 32 threads,
-// 16 primitive quartets per batch, 5 slot(s), 1 accumulators per thread, 10496 B shared per block.
+// roots 2, contracted block: 6, outputs: 6: a lane-split kernel, the lanes' primitive quartets by
+// Rys quadrature with the 2-D tables in registers.
 #include "../rys_common.cuh"
 
 namespace molints {
 
-struct C_dsss {
-    static constexpr int LA = 2, LB = 0, LC = 0, LD = 0;
-    static constexpr int E = 2, F = 0, NR = 2;
-    static constexpr int NA = 6, NC = 1, NBLK = 6;
-    static constexpr int NB = 1, ND = 1;
-    static constexpr int NAB = 6, NCD = 1;
-    static constexpr int G = 32, NPB = 16, NSLOT = 5, ACC = 1;
-    static constexpr int S = 3;
-    static constexpr int SMEM_GROUP = 328;
-    static constexpr bool COL = false;
-    template <typename T, typename A>
-    __device__ __forceinline__ static void col_update(const T *, const T *, const T *, A *) {}
-};
-
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_dsss[6] = {
-    2, 257, 65537, 512, 65792, 131072,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_dsss[7] = {
-    0, 1, 2, 3, 4, 5, 6,
-};
-__device__ const uint32_t kBraTerm_dsss[6] = {
-    65536, 65537, 65538, 65539, 65540, 65541,
-};
-__device__ const uint16_t kKetOff_dsss[2] = {
-    0, 1,
-};
-__device__ const uint32_t kKetTerm_dsss[1] = {
-    65536,
-};
-__device__ const double kNormAB_dsss[6] = {
-    0.5773502691896258, 1.0, 1.0, 0.5773502691896258,
-    1.0, 0.5773502691896258,
-};
-__device__ const double kNormCD_dsss[1] = {
-    1.0,
-};
-
-
-__device__ __forceinline__ RysClassTabs tabs_dsss() {
-    return RysClassTabs{kBlk_dsss, kBraOff_dsss, kBraTerm_dsss, kKetOff_dsss, kKetTerm_dsss,
-                        kNormAB_dsss, kNormCD_dsss, nullptr};
-}
-
-template <int MIXED>
-__global__ void __launch_bounds__(128) rys_queue_dsss(const EriQueue Q, const RysTab R) {
-    rys_queue_body<C_dsss, MIXED>(Q, R, tabs_dsss());
-}
-
-static void rys_prepare_dsss() {
-    static bool done[64] = {false};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_dsss<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 10496);
-
-
-        done[dev] = true;
+// The contracted [e0|f0] block of bra pair p and ket pair q into acc[6] by the 2-point Rys
+// rule, summed over the bra primitive pairs i0, i0 + istep, ... < i1 and the ket primitive pairs
+// j0, j0 + jstep, ... < j1; loop order and splits as in the HGP kernel of the class.
+__device__ __forceinline__ void vrr_dsss_rys(const PairTab &P, const RysTab &R, int p, int q, int i0, int i1,
+                                          int istep, int j0, int j1, int jstep, double *__restrict__ acc) {
+    const int4 ib_ = __ldg(&P.info[p]);
+    const int4 ik_ = __ldg(&P.info[q]);
+#pragma unroll
+    for (int x = 0; x < 6; ++x) acc[x] = 0.0;
+    for (int j = j0; j < j1; j += jstep) {
+        const PrimPair ket = load_pp(P.pp, ik_.x + j);
+        for (int i = i0; i < i1; i += istep) {
+            const PrimPair bra = load_pp(P.pp, ib_.x + i);
+            const double r = rsqrt(bra.zeta + ket.zeta);
+            const double r2 = r * r;
+            const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
+            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double pref = bra.kab * ket.kab * r;
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+#pragma unroll 1
+            for (int k = 0; k < 2; ++k) {
+                double u, w;
+                rys_root<2>(R, T, k, u, w);
+                const double b10 = bra.oo2z * fma(-ez, u, 1.0), b01 = ket.oo2z * fma(-zz, u, 1.0), b00 = 0.5 * r2 * u;
+                (void)b10; (void)b01; (void)b00;
+                const double Cx = fma(-ez * PQx, u, bra.pax), Dx = fma(zz * PQx, u, ket.pax);
+                (void)Cx; (void)Dx;
+                const double Cy = fma(-ez * PQy, u, bra.pay), Dy = fma(zz * PQy, u, ket.pay);
+                (void)Cy; (void)Dy;
+                const double Cz = fma(-ez * PQz, u, bra.paz), Dz = fma(zz * PQz, u, ket.paz);
+                (void)Cz; (void)Dz;
+                const double x0_0 = pref * w;
+                const double x1_0 = Cx * x0_0;
+                const double x2_0 = Cx * x1_0 + 1.0 * b10 * x0_0;
+                const double y0_0 = 1.0;
+                const double y1_0 = Cy * y0_0;
+                const double y2_0 = Cy * y1_0 + 1.0 * b10 * y0_0;
+                const double z0_0 = 1.0;
+                const double z1_0 = Cz * z0_0;
+                const double z2_0 = Cz * z1_0 + 1.0 * b10 * z0_0;
+                acc[0] = fma(x2_0 * y0_0, z0_0, acc[0]);
+                acc[1] = fma(x1_0 * y1_0, z0_0, acc[1]);
+                acc[2] = fma(x1_0 * y0_0, z1_0, acc[2]);
+                acc[3] = fma(x0_0 * y2_0, z0_0, acc[3]);
+                acc[4] = fma(x0_0 * y1_0, z1_0, acc[4]);
+                acc[5] = fma(x0_0 * y0_0, z2_0, acc[5]);
+            }
+        }
     }
 }
 
-// grid_max: resident blocks on the device; the grid is cut to the chunks' groups.
-void launch_rys_dsss(const EriQueue &Q, const RysTab &R, int mixed, int grid_max, cudaStream_t s) {
-    if (Q.nchunks <= 0 || grid_max <= 0) return;
-    rys_prepare_dsss();
-    constexpr int ng = 128 / C_dsss::G;
-    const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    (void)mixed;  // no FP32 variant for this class
-    rys_queue_dsss<0><<<grid, 128, 10496, s>>>(Q, R);
+// Bra and ket HRR of the contracted block (src/HGP.jl:92-114), then the component norms:
+// the normalised (ab|cd) of bra pair p and ket pair q into res[6] (ma, mb, mc, md
+// row-major).
+__device__ __forceinline__ void hrr_dsss_rys(const PairTab &P, int p, int q, const double *__restrict__ acc,
+                                          double *__restrict__ res) {
+    const double4 gb = ldg4(&P.geo[p]);
+    const double4 gk = ldg4(&P.geo[q]);
+    const double ABx = gb.x, ABy = gb.y, ABz = gb.z;
+    const double CDx = gk.x, CDy = gk.y, CDz = gk.z;
+    (void)ABx; (void)ABy; (void)ABz; (void)CDx; (void)CDy; (void)CDz;
+
+    res[0] = acc[0] * 0.5773502691896258;
+    res[1] = acc[1];
+    res[2] = acc[2];
+    res[3] = acc[3] * 0.5773502691896258;
+    res[4] = acc[4];
+    res[5] = acc[5] * 0.5773502691896258;
+}
+
+
+
+__device__ __forceinline__ void store_dsss_rys(double *__restrict__ out, const int4 ib_, const int4 ik_,
+                                            bool same, const double *__restrict__ res) {
+    const bool dab = ib_.z == ib_.w, dcd = ik_.z == ik_.w;
+    (void)dab; (void)dcd;
+    const long long ij_0_0 = pair_index(ib_.z + 0, ib_.w + 0);
+    const long long ij_1_0 = pair_index(ib_.z + 1, ib_.w + 0);
+    const long long ij_2_0 = pair_index(ib_.z + 2, ib_.w + 0);
+    const long long ij_3_0 = pair_index(ib_.z + 3, ib_.w + 0);
+    const long long ij_4_0 = pair_index(ib_.z + 4, ib_.w + 0);
+    const long long ij_5_0 = pair_index(ib_.z + 5, ib_.w + 0);
+    const long long kl_0_0 = pair_index(ik_.z + 0, ik_.w + 0);
+    { const long long ij = ij_0_0, kl = kl_0_0;
+      if ((!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[0]; }
+    { const long long ij = ij_1_0, kl = kl_0_0;
+      if ((!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[1]; }
+    { const long long ij = ij_2_0, kl = kl_0_0;
+      if ((!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[2]; }
+    { const long long ij = ij_3_0, kl = kl_0_0;
+      if ((!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[3]; }
+    { const long long ij = ij_4_0, kl = kl_0_0;
+      if ((!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[4]; }
+    { const long long ij = ij_5_0, kl = kl_0_0;
+      if ((!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[5]; }
+}
+
+// The quartet's unique integrals digested into J and K (molints_plan_jk) instead of stored.
+__device__ __noinline__ void jk_dsss_rys(const JKOut &jk, const int4 ib_, const int4 ik_, bool same,
+                                      const double *__restrict__ res) {
+    const bool dab = ib_.z == ib_.w, dcd = ik_.z == ik_.w;
+    for (int x = 0; x < 6; ++x) {
+        const int ia = x / 1, ibb = (x / 1) % 1, ic = (x / 1) % 1, id = x % 1;
+        if ((dab && ia < ibb) || (dcd && ic < id)) continue;
+        const int i = ib_.z + ia, j = ib_.w + ibb, k = ik_.z + ic, l = ik_.w + id;
+        if (same && pair_index(i, j) < pair_index(k, l)) continue;
+        jk_add(jk, i, j, k, l, res[x]);
+    }
+}
+
+// Persistent work-queue kernel: each warp takes chunks (one bra pair, a run of consecutive
+// ket pairs of one molecule) from a shared counter until the chunk list, ordered by
+// decreasing estimated cost, is exhausted.  A chunk's count field carries the split in bits
+// 16+: lg = log2 S (bits 16-18) and lgj = log2 Sj (bits 20-22).  S lanes share each quartet:
+// lane l takes ket pair q0 + l % (32/S) (+ 32/S per round); its group rank s = l / (32/S)
+// takes every Sj-th ket primitive from s % Sj and every (S/Sj)-th bra primitive from s / Sj.
+// The S partial blocks are summed by a fixed butterfly (the result depends on the split
+// alone, not on the chunk), and the group's first lane runs the HRR and stores.  Heavy
+// quartets are split so that no single lane's serial primitive loop sets the kernel time.
+// JK: digest into J and K (molints_plan_jk) instead of storing the packed integrals; a separate
+// instantiation, so that the store kernels carry none of the digestion code.
+template <int MIXED, int JK>
+__global__ void __launch_bounds__(128) eri_queue_dsss_rys(const EriQueue Q) {
+    const int lane = threadIdx.x & 31;
+    for (;;) {
+        int c = 0;
+        if (lane == 0) c = atomicAdd(Q.counter, 1);
+        c = __shfl_sync(0xffffffffu, c, 0);
+        if (c >= Q.nchunks) return;
+        const int4 ch = __ldg(&Q.chunks[c]);
+        const int p = ch.x, cnt = ch.z & 0xffff, lg = (ch.z >> 16) & 7, lgj = (ch.z >> 20) & 7;
+        const int W = 32 >> lg, kq = lane & (W - 1), s = lane >> (5 - lg);
+        const int js = s & ((1 << lgj) - 1), is = s >> lgj;
+        for (int base = 0; base < cnt; base += W) {
+        const int q = ch.y + base + kq;
+        const bool live = base + kq < cnt;
+        double acc[6];
+        double2 bp = make_double2(0.0, 0.0), bq = bp;
+        if (live) {
+            bp = __ldg(&Q.pairs.bnd[p]);
+            bq = __ldg(&Q.pairs.bnd[q]);
+        }
+        if (!live || bp.x * bq.x < Q.screen_cut) {
+#pragma unroll
+            for (int x = 0; x < 6; ++x) acc[x] = 0.0;
+        } else {
+            const int nb = __ldg(&Q.pairs.info[p]).y, nk = __ldg(&Q.pairs.info[q]).y;
+            vrr_dsss_rys(Q.pairs, Q.rys, p, q, is, nb, 1 << (lg - lgj), js, nk, 1 << lgj, acc);
+        }
+        if (lg) {
+            for (int off = W; off < 32; off <<= 1) {
+#pragma unroll
+                for (int x = 0; x < 6; ++x) acc[x] += __shfl_xor_sync(0xffffffffu, acc[x], off);
+            }
+        }
+        const bool lead = live && s == 0;
+        if (!JK && Q.scratch) {
+            // two-phase: the leaders' HRR writes the blocks of the chunk's quartets straight
+            // into shared memory, where they lie as in the scratch (consecutive slots); the warp
+            // then copies them out as one contiguous run
+            extern __shared__ double stg[];  // 4 * 32 * 6 doubles (launch_eri_dsss_rys)
+            double *sb = stg + (threadIdx.x >> 5) * (32 * 6);
+            if (lead) hrr_dsss_rys(Q.pairs, p, q, acc, sb + kq * 6);
+            __syncwarp();
+            const int nlive = min(W, cnt - base);
+            double *__restrict__ dst = Q.scratch + __ldg(&Q.region[ch.w * kRegionFields]) +
+                (__ldg(&Q.chunk_slot[c]) + base) * (long long)6;
+            for (int t = lane; t < nlive * 6; t += 32) dst[t] = sb[t];
+            __syncwarp();
+        } else if (lead) {
+            double res[6];
+            hrr_dsss_rys(Q.pairs, p, q, acc, res);
+            if constexpr (JK) {
+                jk_dsss_rys(Q.jk, __ldg(&Q.pairs.info[p]), __ldg(&Q.pairs.info[q]), p == q, res);
+            } else {
+                store_dsss_rys(Q.out + __ldg(&Q.mol_out[ch.w]), __ldg(&Q.pairs.info[p]), __ldg(&Q.pairs.info[q]),
+                            p == q, res);
+            }
+        }
+        }
+    }
+}
+
+
+void launch_rys_dsss(const EriQueue &Q0, const RysTab &R, int mixed, int grid, cudaStream_t s) {
+    EriQueue Q = Q0;
+    Q.rys = R;
+    if (Q.nchunks <= 0 || grid <= 0) return;
+    // two-phase plans stage the chunk's blocks in 6144 bytes of dynamic shared memory
+    const size_t smem = Q.scratch && !Q.jk.J ? 6144 : 0;
+    (void)mixed;  // no FP32 variant for this class (MIXED_MIN_VRR)
+    if (Q.jk.J) eri_queue_dsss_rys<0, 1><<<grid, 128, 0, s>>>(Q);
+    else eri_queue_dsss_rys<0, 0><<<grid, 128, smem, s>>>(Q);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_dsss(int mixed) {
-    rys_prepare_dsss();
+
     int n = 0;
     (void)mixed;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dsss<0>, 128, 10496);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, eri_queue_dsss_rys<0, 0>, 128, 0);
     return n;
 }
 

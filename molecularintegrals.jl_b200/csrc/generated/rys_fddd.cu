@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (fd|dd).  Do not edit.
-// roots 5, block 46 x 31, outputs 60 x 36, group 32 threads,
-// 6 primitive quartets per batch, 1 slot(s), 1 accumulators per thread, 106432 B shared per block, column mode.
+// roots 5, block 46 x 31, outputs 60 x 36, group 32 threads, 1 ket pairs a round,
+// 6 primitive quartets per ket pair and batch, 130560 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,11 +11,10 @@ struct C_fddd {
     static constexpr int NA = 46, NC = 31, NBLK = 1426;
     static constexpr int NB = 6, ND = 6;
     static constexpr int NAB = 60, NCD = 36;
-    static constexpr int G = 32, NPB = 6, NSLOT = 1, ACC = 1;
-    static constexpr int S = 30;
-    static constexpr int SMEM_GROUP = 3326;
-    static constexpr bool COL = true;
-    // stage 2, column mode: acc[row] += x[ax] y[ay] z[az] for the column's table columns
+    static constexpr int G = 32, W = 1, H = 1, PB = 6;
+    static constexpr int S = 30, SI = 91, NCP = 31, NCDP = 37;
+    static constexpr int SMEM_GROUP = 4080;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
     __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
         acc[0] = fma(x[3] * y[0], z[0], acc[0]);
@@ -65,179 +64,319 @@ struct C_fddd {
         acc[44] = fma(x[0] * y[1], z[4], acc[44]);
         acc[45] = fma(x[0] * y[0], z[5], acc[45]);
     }
-    static constexpr int NCOLS = 31;
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[10], in[25]);
+        const double h1 = fma(x, in[0], in[10]);
+        const double h2 = fma(x, h1, h0);
+        const double h3 = fma(y, in[10], in[26]);
+        const double h4 = fma(y, in[0], in[11]);
+        const double h5 = fma(x, h4, h3);
+        const double h6 = fma(z, in[10], in[27]);
+        const double h7 = fma(z, in[0], in[12]);
+        const double h8 = fma(x, h7, h6);
+        const double h9 = fma(y, in[11], in[28]);
+        const double h10 = fma(y, h4, h9);
+        const double h11 = fma(z, in[11], in[29]);
+        const double h12 = fma(y, h7, h11);
+        const double h13 = fma(z, in[12], in[30]);
+        const double h14 = fma(z, h7, h13);
+        const double h15 = fma(x, in[11], in[26]);
+        const double h16 = fma(x, in[1], in[11]);
+        const double h17 = fma(x, h16, h15);
+        const double h18 = fma(y, in[1], in[13]);
+        const double h19 = fma(x, h18, h9);
+        const double h20 = fma(z, in[1], in[14]);
+        const double h21 = fma(x, h20, h11);
+        const double h22 = fma(y, in[13], in[31]);
+        const double h23 = fma(y, h18, h22);
+        const double h24 = fma(z, in[13], in[32]);
+        const double h25 = fma(y, h20, h24);
+        const double h26 = fma(z, in[14], in[33]);
+        const double h27 = fma(z, h20, h26);
+        const double h28 = fma(x, in[12], in[27]);
+        const double h29 = fma(x, in[2], in[12]);
+        const double h30 = fma(x, h29, h28);
+        const double h31 = fma(y, in[12], in[29]);
+        const double h32 = fma(y, in[2], in[14]);
+        const double h33 = fma(x, h32, h31);
+        const double h34 = fma(z, in[2], in[15]);
+        const double h35 = fma(x, h34, h13);
+        const double h36 = fma(y, in[14], in[32]);
+        const double h37 = fma(y, h32, h36);
+        const double h38 = fma(y, h34, h26);
+        const double h39 = fma(z, in[15], in[34]);
+        const double h40 = fma(z, h34, h39);
+        const double h41 = fma(x, in[13], in[28]);
+        const double h42 = fma(x, in[3], in[13]);
+        const double h43 = fma(x, h42, h41);
+        const double h44 = fma(y, in[3], in[16]);
+        const double h45 = fma(x, h44, h22);
+        const double h46 = fma(z, in[3], in[17]);
+        const double h47 = fma(x, h46, h24);
+        const double h48 = fma(y, in[16], in[35]);
+        const double h49 = fma(y, h44, h48);
+        const double h50 = fma(z, in[16], in[36]);
+        const double h51 = fma(y, h46, h50);
+        const double h52 = fma(z, in[17], in[37]);
+        const double h53 = fma(z, h46, h52);
+        const double h54 = fma(x, in[15], in[30]);
+        const double h55 = fma(x, in[4], in[15]);
+        const double h56 = fma(x, h55, h54);
+        const double h57 = fma(y, in[15], in[33]);
+        const double h58 = fma(y, in[4], in[18]);
+        const double h59 = fma(x, h58, h57);
+        const double h60 = fma(z, in[4], in[19]);
+        const double h61 = fma(x, h60, h39);
+        const double h62 = fma(y, in[18], in[37]);
+        const double h63 = fma(y, h58, h62);
+        const double h64 = fma(z, in[18], in[38]);
+        const double h65 = fma(y, h60, h64);
+        const double h66 = fma(z, in[19], in[39]);
+        const double h67 = fma(z, h60, h66);
+        const double h68 = fma(x, in[14], in[29]);
+        const double h69 = fma(x, in[5], in[14]);
+        const double h70 = fma(x, h69, h68);
+        const double h71 = fma(y, in[5], in[17]);
+        const double h72 = fma(x, h71, h36);
+        const double h73 = fma(z, in[5], in[18]);
+        const double h74 = fma(x, h73, h26);
+        const double h75 = fma(y, in[17], in[36]);
+        const double h76 = fma(y, h71, h75);
+        const double h77 = fma(y, h73, h52);
+        const double h78 = fma(z, h73, h64);
+        const double h79 = fma(x, in[16], in[31]);
+        const double h80 = fma(x, in[6], in[16]);
+        const double h81 = fma(x, h80, h79);
+        const double h82 = fma(y, in[6], in[20]);
+        const double h83 = fma(x, h82, h48);
+        const double h84 = fma(z, in[6], in[21]);
+        const double h85 = fma(x, h84, h50);
+        const double h86 = fma(y, in[20], in[40]);
+        const double h87 = fma(y, h82, h86);
+        const double h88 = fma(z, in[20], in[41]);
+        const double h89 = fma(y, h84, h88);
+        const double h90 = fma(z, in[21], in[42]);
+        const double h91 = fma(z, h84, h90);
+        const double h92 = fma(x, in[17], in[32]);
+        const double h93 = fma(x, in[7], in[17]);
+        const double h94 = fma(x, h93, h92);
+        const double h95 = fma(y, in[7], in[21]);
+        const double h96 = fma(x, h95, h75);
+        const double h97 = fma(z, in[7], in[22]);
+        const double h98 = fma(x, h97, h52);
+        const double h99 = fma(y, in[21], in[41]);
+        const double h100 = fma(y, h95, h99);
+        const double h101 = fma(y, h97, h90);
+        const double h102 = fma(z, in[22], in[43]);
+        const double h103 = fma(z, h97, h102);
+        const double h104 = fma(x, in[18], in[33]);
+        const double h105 = fma(x, in[8], in[18]);
+        const double h106 = fma(x, h105, h104);
+        const double h107 = fma(y, in[8], in[22]);
+        const double h108 = fma(x, h107, h62);
+        const double h109 = fma(z, in[8], in[23]);
+        const double h110 = fma(x, h109, h64);
+        const double h111 = fma(y, in[22], in[42]);
+        const double h112 = fma(y, h107, h111);
+        const double h113 = fma(y, h109, h102);
+        const double h114 = fma(z, in[23], in[44]);
+        const double h115 = fma(z, h109, h114);
+        const double h116 = fma(x, in[19], in[34]);
+        const double h117 = fma(x, in[9], in[19]);
+        const double h118 = fma(x, h117, h116);
+        const double h119 = fma(y, in[19], in[38]);
+        const double h120 = fma(y, in[9], in[23]);
+        const double h121 = fma(x, h120, h119);
+        const double h122 = fma(z, in[9], in[24]);
+        const double h123 = fma(x, h122, h66);
+        const double h124 = fma(y, in[23], in[43]);
+        const double h125 = fma(y, h120, h124);
+        const double h126 = fma(y, h122, h114);
+        const double h127 = fma(z, in[24], in[45]);
+        const double h128 = fma(z, h122, h127);
+        out[0] = h2;
+        out[31] = h5;
+        out[62] = h8;
+        out[93] = h10;
+        out[124] = h12;
+        out[155] = h14;
+        out[186] = h17;
+        out[217] = h19;
+        out[248] = h21;
+        out[279] = h23;
+        out[310] = h25;
+        out[341] = h27;
+        out[372] = h30;
+        out[403] = h33;
+        out[434] = h35;
+        out[465] = h37;
+        out[496] = h38;
+        out[527] = h40;
+        out[558] = h43;
+        out[589] = h45;
+        out[620] = h47;
+        out[651] = h49;
+        out[682] = h51;
+        out[713] = h53;
+        out[744] = h56;
+        out[775] = h59;
+        out[806] = h61;
+        out[837] = h63;
+        out[868] = h65;
+        out[899] = h67;
+        out[930] = h70;
+        out[961] = h72;
+        out[992] = h74;
+        out[1023] = h76;
+        out[1054] = h77;
+        out[1085] = h78;
+        out[1116] = h81;
+        out[1147] = h83;
+        out[1178] = h85;
+        out[1209] = h87;
+        out[1240] = h89;
+        out[1271] = h91;
+        out[1302] = h94;
+        out[1333] = h96;
+        out[1364] = h98;
+        out[1395] = h100;
+        out[1426] = h101;
+        out[1457] = h103;
+        out[1488] = h106;
+        out[1519] = h108;
+        out[1550] = h110;
+        out[1581] = h112;
+        out[1612] = h113;
+        out[1643] = h115;
+        out[1674] = h118;
+        out[1705] = h121;
+        out[1736] = h123;
+        out[1767] = h125;
+        out[1798] = h126;
+        out[1829] = h128;
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[6], in[16]);
+        const double h1 = fma(x, in[0], in[6]);
+        const double h2 = fma(x, h1, h0);
+        const double h3 = fma(y, in[6], in[17]);
+        const double h4 = fma(y, in[0], in[7]);
+        const double h5 = fma(x, h4, h3);
+        const double h6 = fma(z, in[6], in[18]);
+        const double h7 = fma(z, in[0], in[8]);
+        const double h8 = fma(x, h7, h6);
+        const double h9 = fma(y, in[7], in[19]);
+        const double h10 = fma(y, h4, h9);
+        const double h11 = fma(z, in[7], in[20]);
+        const double h12 = fma(y, h7, h11);
+        const double h13 = fma(z, in[8], in[21]);
+        const double h14 = fma(z, h7, h13);
+        const double h15 = fma(x, in[7], in[17]);
+        const double h16 = fma(x, in[1], in[7]);
+        const double h17 = fma(x, h16, h15);
+        const double h18 = fma(y, in[1], in[9]);
+        const double h19 = fma(x, h18, h9);
+        const double h20 = fma(z, in[1], in[11]);
+        const double h21 = fma(x, h20, h11);
+        const double h22 = fma(y, in[9], in[22]);
+        const double h23 = fma(y, h18, h22);
+        const double h24 = fma(z, in[9], in[23]);
+        const double h25 = fma(y, h20, h24);
+        const double h26 = fma(z, in[11], in[24]);
+        const double h27 = fma(z, h20, h26);
+        const double h28 = fma(x, in[8], in[18]);
+        const double h29 = fma(x, in[2], in[8]);
+        const double h30 = fma(x, h29, h28);
+        const double h31 = fma(y, in[8], in[20]);
+        const double h32 = fma(y, in[2], in[11]);
+        const double h33 = fma(x, h32, h31);
+        const double h34 = fma(z, in[2], in[10]);
+        const double h35 = fma(x, h34, h13);
+        const double h36 = fma(y, in[11], in[23]);
+        const double h37 = fma(y, h32, h36);
+        const double h38 = fma(y, h34, h26);
+        const double h39 = fma(z, in[10], in[25]);
+        const double h40 = fma(z, h34, h39);
+        const double h41 = fma(x, in[9], in[19]);
+        const double h42 = fma(x, in[3], in[9]);
+        const double h43 = fma(x, h42, h41);
+        const double h44 = fma(y, in[3], in[12]);
+        const double h45 = fma(x, h44, h22);
+        const double h46 = fma(z, in[3], in[13]);
+        const double h47 = fma(x, h46, h24);
+        const double h48 = fma(y, in[12], in[26]);
+        const double h49 = fma(y, h44, h48);
+        const double h50 = fma(z, in[12], in[27]);
+        const double h51 = fma(y, h46, h50);
+        const double h52 = fma(z, in[13], in[28]);
+        const double h53 = fma(z, h46, h52);
+        const double h54 = fma(x, in[11], in[20]);
+        const double h55 = fma(x, in[4], in[11]);
+        const double h56 = fma(x, h55, h54);
+        const double h57 = fma(y, in[4], in[13]);
+        const double h58 = fma(x, h57, h36);
+        const double h59 = fma(z, in[4], in[14]);
+        const double h60 = fma(x, h59, h26);
+        const double h61 = fma(y, in[13], in[27]);
+        const double h62 = fma(y, h57, h61);
+        const double h63 = fma(y, h59, h52);
+        const double h64 = fma(z, in[14], in[29]);
+        const double h65 = fma(z, h59, h64);
+        const double h66 = fma(x, in[10], in[21]);
+        const double h67 = fma(x, in[5], in[10]);
+        const double h68 = fma(x, h67, h66);
+        const double h69 = fma(y, in[10], in[24]);
+        const double h70 = fma(y, in[5], in[14]);
+        const double h71 = fma(x, h70, h69);
+        const double h72 = fma(z, in[5], in[15]);
+        const double h73 = fma(x, h72, h39);
+        const double h74 = fma(y, in[14], in[28]);
+        const double h75 = fma(y, h70, h74);
+        const double h76 = fma(y, h72, h64);
+        const double h77 = fma(z, in[15], in[30]);
+        const double h78 = fma(z, h72, h77);
+        out[0] = h2 * (nrm * 0.3333333333333334);
+        out[1] = h5 * (nrm * 0.5773502691896258);
+        out[2] = h8 * (nrm * 0.5773502691896258);
+        out[3] = h10 * (nrm * 0.3333333333333334);
+        out[4] = h12 * (nrm * 0.5773502691896258);
+        out[5] = h14 * (nrm * 0.3333333333333334);
+        out[6] = h17 * (nrm * 0.5773502691896258);
+        out[7] = h19 * (nrm * 1.0);
+        out[8] = h21 * (nrm * 1.0);
+        out[9] = h23 * (nrm * 0.5773502691896258);
+        out[10] = h25 * (nrm * 1.0);
+        out[11] = h27 * (nrm * 0.5773502691896258);
+        out[12] = h30 * (nrm * 0.5773502691896258);
+        out[13] = h33 * (nrm * 1.0);
+        out[14] = h35 * (nrm * 1.0);
+        out[15] = h37 * (nrm * 0.5773502691896258);
+        out[16] = h38 * (nrm * 1.0);
+        out[17] = h40 * (nrm * 0.5773502691896258);
+        out[18] = h43 * (nrm * 0.3333333333333334);
+        out[19] = h45 * (nrm * 0.5773502691896258);
+        out[20] = h47 * (nrm * 0.5773502691896258);
+        out[21] = h49 * (nrm * 0.3333333333333334);
+        out[22] = h51 * (nrm * 0.5773502691896258);
+        out[23] = h53 * (nrm * 0.3333333333333334);
+        out[24] = h56 * (nrm * 0.5773502691896258);
+        out[25] = h58 * (nrm * 1.0);
+        out[26] = h60 * (nrm * 1.0);
+        out[27] = h62 * (nrm * 0.5773502691896258);
+        out[28] = h63 * (nrm * 1.0);
+        out[29] = h65 * (nrm * 0.5773502691896258);
+        out[30] = h68 * (nrm * 0.3333333333333334);
+        out[31] = h71 * (nrm * 0.5773502691896258);
+        out[32] = h73 * (nrm * 0.5773502691896258);
+        out[33] = h75 * (nrm * 0.3333333333333334);
+        out[34] = h76 * (nrm * 0.5773502691896258);
+        out[35] = h78 * (nrm * 0.3333333333333334);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_fddd[1426] = {
-    17, 272, 65552, 527, 65807, 131087, 18, 273, 65553, 528, 131088, 65808,
-    783, 66063, 131343, 196623, 19, 274, 65554, 529, 65809, 131089, 784, 66064,
-    131344, 196624, 1039, 66319, 131599, 196879, 262159, 1292, 1547, 66827, 1802, 67082,
-    132362, 1293, 1548, 66828, 1803, 132363, 67083, 2058, 67338, 132618, 197898, 1294,
-    1549, 66829, 1804, 67084, 132364, 2059, 67339, 132619, 197899, 2314, 67594, 132874,
-    198154, 263434, 327692, 327947, 393227, 328202, 393482, 458762, 327693, 327948, 393228, 328203,
-    458763, 393483, 328458, 393738, 459018, 524298, 327694, 327949, 393229, 328204, 393484, 458764,
-    328459, 393739, 459019, 524299, 328714, 393994, 459274, 524554, 589834, 2567, 2822, 68102,
-    3077, 68357, 133637, 2568, 2823, 68103, 3078, 133638, 68358, 3333, 68613, 133893,
-    199173, 2569, 2824, 68104, 3079, 68359, 133639, 3334, 68614, 133894, 199174, 3589,
-    68869, 134149, 199429, 264709, 655367, 655622, 720902, 655877, 721157, 786437, 655368, 655623,
-    720903, 655878, 786438, 721158, 656133, 721413, 786693, 851973, 655369, 655624, 720904, 655879,
-    721159, 786439, 656134, 721414, 786694, 851974, 656389, 721669, 786949, 852229, 917509, 328967,
-    329222, 394502, 329477, 394757, 460037, 328968, 329223, 394503, 329478, 460038, 394758, 329733,
-    395013, 460293, 525573, 328969, 329224, 394504, 329479, 394759, 460039, 329734, 395014, 460294,
-    525574, 329989, 395269, 460549, 525829, 591109, 3842, 4097, 69377, 4352, 69632, 134912,
-    3843, 4098, 69378, 4353, 134913, 69633, 4608, 69888, 135168, 200448, 3844, 4099,
-    69379, 4354, 69634, 134914, 4609, 69889, 135169, 200449, 4864, 70144, 135424, 200704,
-    265984, 330242, 330497, 395777, 330752, 396032, 461312, 330243, 330498, 395778, 330753, 461313,
-    396033, 331008, 396288, 461568, 526848, 330244, 330499, 395779, 330754, 396034, 461314, 331009,
-    396289, 461569, 526849, 331264, 396544, 461824, 527104, 592384, 656642, 656897, 722177, 657152,
-    722432, 787712, 656643, 656898, 722178, 657153, 787713, 722433, 657408, 722688, 787968, 853248,
-    656644, 656899, 722179, 657154, 722434, 787714, 657409, 722689, 787969, 853249, 657664, 722944,
-    788224, 853504, 918784, 983042, 983297, 1048577, 983552, 1048832, 1114112, 983043, 983298, 1048578,
-    983553, 1114113, 1048833, 983808, 1049088, 1114368, 1179648, 983044, 983299, 1048579, 983554, 1048834,
-    1114114, 983809, 1049089, 1114369, 1179649, 984064, 1049344, 1114624, 1179904, 1245184, 22, 277,
-    65557, 532, 65812, 131092, 23, 278, 65558, 533, 131093, 65813, 788, 66068,
-    131348, 196628, 24, 279, 65559, 534, 65814, 131094, 789, 66069, 131349, 196629,
-    1044, 66324, 131604, 196884, 262164, 1297, 1552, 66832, 1807, 67087, 132367, 1298,
-    1553, 66833, 1808, 132368, 67088, 2063, 67343, 132623, 197903, 1299, 1554, 66834,
-    1809, 67089, 132369, 2064, 67344, 132624, 197904, 2319, 67599, 132879, 198159, 263439,
-    327697, 327952, 393232, 328207, 393487, 458767, 327698, 327953, 393233, 328208, 458768, 393488,
-    328463, 393743, 459023, 524303, 327699, 327954, 393234, 328209, 393489, 458769, 328464, 393744,
-    459024, 524304, 328719, 393999, 459279, 524559, 589839, 2572, 2827, 68107, 3082, 68362,
-    133642, 2573, 2828, 68108, 3083, 133643, 68363, 3338, 68618, 133898, 199178, 2574,
-    2829, 68109, 3084, 68364, 133644, 3339, 68619, 133899, 199179, 3594, 68874, 134154,
-    199434, 264714, 328972, 329227, 394507, 329482, 394762, 460042, 328973, 329228, 394508, 329483,
-    460043, 394763, 329738, 395018, 460298, 525578, 328974, 329229, 394509, 329484, 394764, 460044,
-    329739, 395019, 460299, 525579, 329994, 395274, 460554, 525834, 591114, 655372, 655627, 720907,
-    655882, 721162, 786442, 655373, 655628, 720908, 655883, 786443, 721163, 656138, 721418, 786698,
-    851978, 655374, 655629, 720909, 655884, 721164, 786444, 656139, 721419, 786699, 851979, 656394,
-    721674, 786954, 852234, 917514, 3847, 4102, 69382, 4357, 69637, 134917, 3848, 4103,
-    69383, 4358, 134918, 69638, 4613, 69893, 135173, 200453, 3849, 4104, 69384, 4359,
-    69639, 134919, 4614, 69894, 135174, 200454, 4869, 70149, 135429, 200709, 265989, 330247,
-    330502, 395782, 330757, 396037, 461317, 330248, 330503, 395783, 330758, 461318, 396038, 331013,
-    396293, 461573, 526853, 330249, 330504, 395784, 330759, 396039, 461319, 331014, 396294, 461574,
-    526854, 331269, 396549, 461829, 527109, 592389, 656647, 656902, 722182, 657157, 722437, 787717,
-    656648, 656903, 722183, 657158, 787718, 722438, 657413, 722693, 787973, 853253, 656649, 656904,
-    722184, 657159, 722439, 787719, 657414, 722694, 787974, 853254, 657669, 722949, 788229, 853509,
-    918789, 983047, 983302, 1048582, 983557, 1048837, 1114117, 983048, 983303, 1048583, 983558, 1114118,
-    1048838, 983813, 1049093, 1114373, 1179653, 983049, 983304, 1048584, 983559, 1048839, 1114119, 983814,
-    1049094, 1114374, 1179654, 984069, 1049349, 1114629, 1179909, 1245189, 5122, 5377, 70657, 5632,
-    70912, 136192, 5123, 5378, 70658, 5633, 136193, 70913, 5888, 71168, 136448, 201728,
-    5124, 5379, 70659, 5634, 70914, 136194, 5889, 71169, 136449, 201729, 6144, 71424,
-    136704, 201984, 267264, 331522, 331777, 397057, 332032, 397312, 462592, 331523, 331778, 397058,
-    332033, 462593, 397313, 332288, 397568, 462848, 528128, 331524, 331779, 397059, 332034, 397314,
-    462594, 332289, 397569, 462849, 528129, 332544, 397824, 463104, 528384, 593664, 657922, 658177,
-    723457, 658432, 723712, 788992, 657923, 658178, 723458, 658433, 788993, 723713, 658688, 723968,
-    789248, 854528, 657924, 658179, 723459, 658434, 723714, 788994, 658689, 723969, 789249, 854529,
-    658944, 724224, 789504, 854784, 920064, 984322, 984577, 1049857, 984832, 1050112, 1115392, 984323,
-    984578, 1049858, 984833, 1115393, 1050113, 985088, 1050368, 1115648, 1180928, 984324, 984579, 1049859,
-    984834, 1050114, 1115394, 985089, 1050369, 1115649, 1180929, 985344, 1050624, 1115904, 1181184, 1246464,
-    1310722, 1310977, 1376257, 1311232, 1376512, 1441792, 1310723, 1310978, 1376258, 1311233, 1441793, 1376513,
-    1311488, 1376768, 1442048, 1507328, 1310724, 1310979, 1376259, 1311234, 1376514, 1441794, 1311489, 1376769,
-    1442049, 1507329, 1311744, 1377024, 1442304, 1507584, 1572864, 27, 282, 65562, 537, 65817,
-    131097, 28, 283, 65563, 538, 131098, 65818, 793, 66073, 131353, 196633, 29,
-    284, 65564, 539, 65819, 131099, 794, 66074, 131354, 196634, 1049, 66329, 131609,
-    196889, 262169, 1302, 1557, 66837, 1812, 67092, 132372, 1303, 1558, 66838, 1813,
-    132373, 67093, 2068, 67348, 132628, 197908, 1304, 1559, 66839, 1814, 67094, 132374,
-    2069, 67349, 132629, 197909, 2324, 67604, 132884, 198164, 263444, 327702, 327957, 393237,
-    328212, 393492, 458772, 327703, 327958, 393238, 328213, 458773, 393493, 328468, 393748, 459028,
-    524308, 327704, 327959, 393239, 328214, 393494, 458774, 328469, 393749, 459029, 524309, 328724,
-    394004, 459284, 524564, 589844, 2577, 2832, 68112, 3087, 68367, 133647, 2578, 2833,
-    68113, 3088, 133648, 68368, 3343, 68623, 133903, 199183, 2579, 2834, 68114, 3089,
-    68369, 133649, 3344, 68624, 133904, 199184, 3599, 68879, 134159, 199439, 264719, 328977,
-    329232, 394512, 329487, 394767, 460047, 328978, 329233, 394513, 329488, 460048, 394768, 329743,
-    395023, 460303, 525583, 328979, 329234, 394514, 329489, 394769, 460049, 329744, 395024, 460304,
-    525584, 329999, 395279, 460559, 525839, 591119, 655377, 655632, 720912, 655887, 721167, 786447,
-    655378, 655633, 720913, 655888, 786448, 721168, 656143, 721423, 786703, 851983, 655379, 655634,
-    720914, 655889, 721169, 786449, 656144, 721424, 786704, 851984, 656399, 721679, 786959, 852239,
-    917519, 3852, 4107, 69387, 4362, 69642, 134922, 3853, 4108, 69388, 4363, 134923,
-    69643, 4618, 69898, 135178, 200458, 3854, 4109, 69389, 4364, 69644, 134924, 4619,
-    69899, 135179, 200459, 4874, 70154, 135434, 200714, 265994, 330252, 330507, 395787, 330762,
-    396042, 461322, 330253, 330508, 395788, 330763, 461323, 396043, 331018, 396298, 461578, 526858,
-    330254, 330509, 395789, 330764, 396044, 461324, 331019, 396299, 461579, 526859, 331274, 396554,
-    461834, 527114, 592394, 656652, 656907, 722187, 657162, 722442, 787722, 656653, 656908, 722188,
-    657163, 787723, 722443, 657418, 722698, 787978, 853258, 656654, 656909, 722189, 657164, 722444,
-    787724, 657419, 722699, 787979, 853259, 657674, 722954, 788234, 853514, 918794, 983052, 983307,
-    1048587, 983562, 1048842, 1114122, 983053, 983308, 1048588, 983563, 1114123, 1048843, 983818, 1049098,
-    1114378, 1179658, 983054, 983309, 1048589, 983564, 1048844, 1114124, 983819, 1049099, 1114379, 1179659,
-    984074, 1049354, 1114634, 1179914, 1245194, 5127, 5382, 70662, 5637, 70917, 136197, 5128,
-    5383, 70663, 5638, 136198, 70918, 5893, 71173, 136453, 201733, 5129, 5384, 70664,
-    5639, 70919, 136199, 5894, 71174, 136454, 201734, 6149, 71429, 136709, 201989, 267269,
-    331527, 331782, 397062, 332037, 397317, 462597, 331528, 331783, 397063, 332038, 462598, 397318,
-    332293, 397573, 462853, 528133, 331529, 331784, 397064, 332039, 397319, 462599, 332294, 397574,
-    462854, 528134, 332549, 397829, 463109, 528389, 593669, 657927, 658182, 723462, 658437, 723717,
-    788997, 657928, 658183, 723463, 658438, 788998, 723718, 658693, 723973, 789253, 854533, 657929,
-    658184, 723464, 658439, 723719, 788999, 658694, 723974, 789254, 854534, 658949, 724229, 789509,
-    854789, 920069, 984327, 984582, 1049862, 984837, 1050117, 1115397, 984328, 984583, 1049863, 984838,
-    1115398, 1050118, 985093, 1050373, 1115653, 1180933, 984329, 984584, 1049864, 984839, 1050119, 1115399,
-    985094, 1050374, 1115654, 1180934, 985349, 1050629, 1115909, 1181189, 1246469, 1310727, 1310982, 1376262,
-    1311237, 1376517, 1441797, 1310728, 1310983, 1376263, 1311238, 1441798, 1376518, 1311493, 1376773, 1442053,
-    1507333, 1310729, 1310984, 1376264, 1311239, 1376519, 1441799, 1311494, 1376774, 1442054, 1507334, 1311749,
-    1377029, 1442309, 1507589, 1572869, 6402, 6657, 71937, 6912, 72192, 137472, 6403, 6658,
-    71938, 6913, 137473, 72193, 7168, 72448, 137728, 203008, 6404, 6659, 71939, 6914,
-    72194, 137474, 7169, 72449, 137729, 203009, 7424, 72704, 137984, 203264, 268544, 332802,
-    333057, 398337, 333312, 398592, 463872, 332803, 333058, 398338, 333313, 463873, 398593, 333568,
-    398848, 464128, 529408, 332804, 333059, 398339, 333314, 398594, 463874, 333569, 398849, 464129,
-    529409, 333824, 399104, 464384, 529664, 594944, 659202, 659457, 724737, 659712, 724992, 790272,
-    659203, 659458, 724738, 659713, 790273, 724993, 659968, 725248, 790528, 855808, 659204, 659459,
-    724739, 659714, 724994, 790274, 659969, 725249, 790529, 855809, 660224, 725504, 790784, 856064,
-    921344, 985602, 985857, 1051137, 986112, 1051392, 1116672, 985603, 985858, 1051138, 986113, 1116673,
-    1051393, 986368, 1051648, 1116928, 1182208, 985604, 985859, 1051139, 986114, 1051394, 1116674, 986369,
-    1051649, 1116929, 1182209, 986624, 1051904, 1117184, 1182464, 1247744, 1312002, 1312257, 1377537, 1312512,
-    1377792, 1443072, 1312003, 1312258, 1377538, 1312513, 1443073, 1377793, 1312768, 1378048, 1443328, 1508608,
-    1312004, 1312259, 1377539, 1312514, 1377794, 1443074, 1312769, 1378049, 1443329, 1508609, 1313024, 1378304,
-    1443584, 1508864, 1574144, 1638402, 1638657, 1703937, 1638912, 1704192, 1769472, 1638403, 1638658, 1703938,
-    1638913, 1769473, 1704193, 1639168, 1704448, 1769728, 1835008, 1638404, 1638659, 1703939, 1638914, 1704194,
-    1769474, 1639169, 1704449, 1769729, 1835009, 1639424, 1704704, 1769984, 1835264, 1900544,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_fddd[61] = {
-    0, 3, 7, 11, 14, 18, 21, 24, 28, 32, 35, 39,
-    42, 45, 49, 53, 56, 60, 63, 66, 70, 74, 77, 81,
-    84, 87, 91, 95, 98, 102, 105, 108, 112, 116, 119, 123,
-    126, 129, 133, 137, 140, 144, 147, 150, 154, 158, 161, 165,
-    168, 171, 175, 179, 182, 186, 189, 192, 196, 200, 203, 207,
-    210,
-};
-__device__ const uint32_t kBraTerm_fddd[210] = {
-    66560, 131338, 65561, 66816, 65803, 66058, 65562, 67072, 65804, 66314, 65563, 67328,
-    131595, 65564, 67584, 66060, 66315, 65565, 67840, 131852, 65566, 66561, 131339, 65562,
-    66817, 65805, 66059, 65564, 67073, 65806, 66315, 65565, 67329, 131597, 65567, 67585,
-    66062, 66317, 65568, 67841, 131854, 65569, 66562, 131340, 65563, 66818, 65806, 66060,
-    65565, 67074, 65807, 66316, 65566, 67330, 131598, 65568, 67586, 66063, 66318, 65569,
-    67842, 131855, 65570, 66563, 131341, 65564, 66819, 65808, 66061, 65567, 67075, 65809,
-    66317, 65568, 67331, 131600, 65571, 67587, 66065, 66320, 65572, 67843, 131857, 65573,
-    66564, 131343, 65566, 66820, 65810, 66063, 65569, 67076, 65811, 66319, 65570, 67332,
-    131602, 65573, 67588, 66067, 66322, 65574, 67844, 131859, 65575, 66565, 131342, 65565,
-    66821, 65809, 66062, 65568, 67077, 65810, 66318, 65569, 67333, 131601, 65572, 67589,
-    66066, 66321, 65573, 67845, 131858, 65574, 66566, 131344, 65567, 66822, 65812, 66064,
-    65571, 67078, 65813, 66320, 65572, 67334, 131604, 65576, 67590, 66069, 66324, 65577,
-    67846, 131861, 65578, 66567, 131345, 65568, 66823, 65813, 66065, 65572, 67079, 65814,
-    66321, 65573, 67335, 131605, 65577, 67591, 66070, 66325, 65578, 67847, 131862, 65579,
-    66568, 131346, 65569, 66824, 65814, 66066, 65573, 67080, 65815, 66322, 65574, 67336,
-    131606, 65578, 67592, 66071, 66326, 65579, 67848, 131863, 65580, 66569, 131347, 65570,
-    66825, 65815, 66067, 65574, 67081, 65816, 66323, 65575, 67337, 131607, 65579, 67593,
-    66072, 66327, 65580, 67849, 131864, 65581,
-};
-__device__ const uint16_t kKetOff_fddd[37] = {
-    0, 3, 7, 11, 14, 18, 21, 24, 28, 32, 35, 39,
-    42, 45, 49, 53, 56, 60, 63, 66, 70, 74, 77, 81,
-    84, 87, 91, 95, 98, 102, 105, 108, 112, 116, 119, 123,
-    126,
-};
-__device__ const uint32_t kKetTerm_fddd[126] = {
-    66560, 131334, 65552, 66816, 65799, 66054, 65553, 67072, 65800, 66310, 65554, 67328,
-    131591, 65555, 67584, 66056, 66311, 65556, 67840, 131848, 65557, 66561, 131335, 65553,
-    66817, 65801, 66055, 65555, 67073, 65803, 66311, 65556, 67329, 131593, 65558, 67585,
-    66059, 66313, 65559, 67841, 131851, 65560, 66562, 131336, 65554, 66818, 65803, 66056,
-    65556, 67074, 65802, 66312, 65557, 67330, 131595, 65559, 67586, 66058, 66315, 65560,
-    67842, 131850, 65561, 66563, 131337, 65555, 66819, 65804, 66057, 65558, 67075, 65805,
-    66313, 65559, 67331, 131596, 65562, 67587, 66061, 66316, 65563, 67843, 131853, 65564,
-    66564, 131339, 65556, 66820, 65805, 66059, 65559, 67076, 65806, 66315, 65560, 67332,
-    131597, 65563, 67588, 66062, 66317, 65564, 67844, 131854, 65565, 66565, 131338, 65557,
-    66821, 65806, 66058, 65560, 67077, 65807, 66314, 65561, 67333, 131598, 65564, 67589,
-    66063, 66318, 65565, 67845, 131855, 65566,
-};
 __device__ const double kNormAB_fddd[60] = {
     0.14907119849998599, 0.2581988897471611, 0.2581988897471611, 0.14907119849998599,
     0.2581988897471611, 0.14907119849998599, 0.3333333333333334, 0.5773502691896258,
@@ -255,25 +394,12 @@ __device__ const double kNormAB_fddd[60] = {
     0.5773502691896258, 0.3333333333333334, 0.14907119849998599, 0.2581988897471611,
     0.2581988897471611, 0.14907119849998599, 0.2581988897471611, 0.14907119849998599,
 };
-__device__ const double kNormCD_fddd[36] = {
-    0.3333333333333334, 0.5773502691896258, 0.5773502691896258, 0.3333333333333334,
-    0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 1.0,
-    1.0, 0.5773502691896258, 1.0, 0.5773502691896258,
-    0.5773502691896258, 1.0, 1.0, 0.5773502691896258,
-    1.0, 0.5773502691896258, 0.3333333333333334, 0.5773502691896258,
-    0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 0.3333333333333334,
-    0.5773502691896258, 1.0, 1.0, 0.5773502691896258,
-    1.0, 0.5773502691896258, 0.3333333333333334, 0.5773502691896258,
-    0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 0.3333333333333334,
-};
-
 
 // column components cx | cy << 4 | cz << 8
 __device__ const uint16_t kCol_fddd[31] = { 2, 17, 257, 32, 272, 512, 3, 18, 258, 33, 513, 273, 48, 288, 528, 768, 4, 19, 259, 34, 274, 514, 49, 289, 529, 769, 64, 304, 544, 784, 1024 };
 
 __device__ __forceinline__ RysClassTabs tabs_fddd() {
-    return RysClassTabs{kBlk_fddd, kBraOff_fddd, kBraTerm_fddd, kKetOff_fddd, kKetTerm_fddd,
-                        kNormAB_fddd, kNormCD_fddd, kCol_fddd};
+    return RysClassTabs{kNormAB_fddd, kCol_fddd};
 }
 
 template <int MIXED>
@@ -286,8 +412,8 @@ static void rys_prepare_fddd() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_fddd<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 106432);
-        cudaFuncSetAttribute(rys_queue_fddd<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 106432);
+        cudaFuncSetAttribute(rys_queue_fddd<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 130560);
+        cudaFuncSetAttribute(rys_queue_fddd<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 130560);
 
         done[dev] = true;
     }
@@ -299,16 +425,16 @@ void launch_rys_fddd(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_fddd();
     constexpr int ng = 128 / C_fddd::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_fddd<1><<<grid, 128, 106432, s>>>(Q, R);
-    else rys_queue_fddd<0><<<grid, 128, 106432, s>>>(Q, R);
+    if (mixed) rys_queue_fddd<1><<<grid, 128, 130560, s>>>(Q, R);
+    else rys_queue_fddd<0><<<grid, 128, 130560, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_fddd(int mixed) {
     rys_prepare_fddd();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fddd<1>, 128, 106432);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fddd<0>, 128, 106432);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fddd<1>, 128, 130560);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fddd<0>, 128, 130560);
     return n;
 }
 

@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (fd|dp).  Do not edit.
-// roots 5, block 46 x 16, outputs 60 x 18, group 32 threads,
-// 6 primitive quartets per batch, 1 slot(s), 1 accumulators per thread, 70400 B shared per block, column mode.
+// roots 5, block 46 x 16, outputs 60 x 18, group 32 threads, 1 ket pairs a round,
+// 5 primitive quartets per ket pair and batch, 69120 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,11 +11,10 @@ struct C_fddp {
     static constexpr int NA = 46, NC = 16, NBLK = 736;
     static constexpr int NB = 6, ND = 3;
     static constexpr int NAB = 60, NCD = 18;
-    static constexpr int G = 32, NPB = 6, NSLOT = 1, ACC = 1;
-    static constexpr int S = 24;
-    static constexpr int SMEM_GROUP = 2200;
-    static constexpr bool COL = true;
-    // stage 2, column mode: acc[row] += x[ax] y[ay] z[az] for the column's table columns
+    static constexpr int G = 32, W = 1, H = 1, PB = 5;
+    static constexpr int S = 24, SI = 73, NCP = 17, NCDP = 19;
+    static constexpr int SMEM_GROUP = 2160;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
     __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
         acc[0] = fma(x[3] * y[0], z[0], acc[0]);
@@ -65,112 +64,240 @@ struct C_fddp {
         acc[44] = fma(x[0] * y[1], z[4], acc[44]);
         acc[45] = fma(x[0] * y[0], z[5], acc[45]);
     }
-    static constexpr int NCOLS = 16;
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[10], in[25]);
+        const double h1 = fma(x, in[0], in[10]);
+        const double h2 = fma(x, h1, h0);
+        const double h3 = fma(y, in[10], in[26]);
+        const double h4 = fma(y, in[0], in[11]);
+        const double h5 = fma(x, h4, h3);
+        const double h6 = fma(z, in[10], in[27]);
+        const double h7 = fma(z, in[0], in[12]);
+        const double h8 = fma(x, h7, h6);
+        const double h9 = fma(y, in[11], in[28]);
+        const double h10 = fma(y, h4, h9);
+        const double h11 = fma(z, in[11], in[29]);
+        const double h12 = fma(y, h7, h11);
+        const double h13 = fma(z, in[12], in[30]);
+        const double h14 = fma(z, h7, h13);
+        const double h15 = fma(x, in[11], in[26]);
+        const double h16 = fma(x, in[1], in[11]);
+        const double h17 = fma(x, h16, h15);
+        const double h18 = fma(y, in[1], in[13]);
+        const double h19 = fma(x, h18, h9);
+        const double h20 = fma(z, in[1], in[14]);
+        const double h21 = fma(x, h20, h11);
+        const double h22 = fma(y, in[13], in[31]);
+        const double h23 = fma(y, h18, h22);
+        const double h24 = fma(z, in[13], in[32]);
+        const double h25 = fma(y, h20, h24);
+        const double h26 = fma(z, in[14], in[33]);
+        const double h27 = fma(z, h20, h26);
+        const double h28 = fma(x, in[12], in[27]);
+        const double h29 = fma(x, in[2], in[12]);
+        const double h30 = fma(x, h29, h28);
+        const double h31 = fma(y, in[12], in[29]);
+        const double h32 = fma(y, in[2], in[14]);
+        const double h33 = fma(x, h32, h31);
+        const double h34 = fma(z, in[2], in[15]);
+        const double h35 = fma(x, h34, h13);
+        const double h36 = fma(y, in[14], in[32]);
+        const double h37 = fma(y, h32, h36);
+        const double h38 = fma(y, h34, h26);
+        const double h39 = fma(z, in[15], in[34]);
+        const double h40 = fma(z, h34, h39);
+        const double h41 = fma(x, in[13], in[28]);
+        const double h42 = fma(x, in[3], in[13]);
+        const double h43 = fma(x, h42, h41);
+        const double h44 = fma(y, in[3], in[16]);
+        const double h45 = fma(x, h44, h22);
+        const double h46 = fma(z, in[3], in[17]);
+        const double h47 = fma(x, h46, h24);
+        const double h48 = fma(y, in[16], in[35]);
+        const double h49 = fma(y, h44, h48);
+        const double h50 = fma(z, in[16], in[36]);
+        const double h51 = fma(y, h46, h50);
+        const double h52 = fma(z, in[17], in[37]);
+        const double h53 = fma(z, h46, h52);
+        const double h54 = fma(x, in[15], in[30]);
+        const double h55 = fma(x, in[4], in[15]);
+        const double h56 = fma(x, h55, h54);
+        const double h57 = fma(y, in[15], in[33]);
+        const double h58 = fma(y, in[4], in[18]);
+        const double h59 = fma(x, h58, h57);
+        const double h60 = fma(z, in[4], in[19]);
+        const double h61 = fma(x, h60, h39);
+        const double h62 = fma(y, in[18], in[37]);
+        const double h63 = fma(y, h58, h62);
+        const double h64 = fma(z, in[18], in[38]);
+        const double h65 = fma(y, h60, h64);
+        const double h66 = fma(z, in[19], in[39]);
+        const double h67 = fma(z, h60, h66);
+        const double h68 = fma(x, in[14], in[29]);
+        const double h69 = fma(x, in[5], in[14]);
+        const double h70 = fma(x, h69, h68);
+        const double h71 = fma(y, in[5], in[17]);
+        const double h72 = fma(x, h71, h36);
+        const double h73 = fma(z, in[5], in[18]);
+        const double h74 = fma(x, h73, h26);
+        const double h75 = fma(y, in[17], in[36]);
+        const double h76 = fma(y, h71, h75);
+        const double h77 = fma(y, h73, h52);
+        const double h78 = fma(z, h73, h64);
+        const double h79 = fma(x, in[16], in[31]);
+        const double h80 = fma(x, in[6], in[16]);
+        const double h81 = fma(x, h80, h79);
+        const double h82 = fma(y, in[6], in[20]);
+        const double h83 = fma(x, h82, h48);
+        const double h84 = fma(z, in[6], in[21]);
+        const double h85 = fma(x, h84, h50);
+        const double h86 = fma(y, in[20], in[40]);
+        const double h87 = fma(y, h82, h86);
+        const double h88 = fma(z, in[20], in[41]);
+        const double h89 = fma(y, h84, h88);
+        const double h90 = fma(z, in[21], in[42]);
+        const double h91 = fma(z, h84, h90);
+        const double h92 = fma(x, in[17], in[32]);
+        const double h93 = fma(x, in[7], in[17]);
+        const double h94 = fma(x, h93, h92);
+        const double h95 = fma(y, in[7], in[21]);
+        const double h96 = fma(x, h95, h75);
+        const double h97 = fma(z, in[7], in[22]);
+        const double h98 = fma(x, h97, h52);
+        const double h99 = fma(y, in[21], in[41]);
+        const double h100 = fma(y, h95, h99);
+        const double h101 = fma(y, h97, h90);
+        const double h102 = fma(z, in[22], in[43]);
+        const double h103 = fma(z, h97, h102);
+        const double h104 = fma(x, in[18], in[33]);
+        const double h105 = fma(x, in[8], in[18]);
+        const double h106 = fma(x, h105, h104);
+        const double h107 = fma(y, in[8], in[22]);
+        const double h108 = fma(x, h107, h62);
+        const double h109 = fma(z, in[8], in[23]);
+        const double h110 = fma(x, h109, h64);
+        const double h111 = fma(y, in[22], in[42]);
+        const double h112 = fma(y, h107, h111);
+        const double h113 = fma(y, h109, h102);
+        const double h114 = fma(z, in[23], in[44]);
+        const double h115 = fma(z, h109, h114);
+        const double h116 = fma(x, in[19], in[34]);
+        const double h117 = fma(x, in[9], in[19]);
+        const double h118 = fma(x, h117, h116);
+        const double h119 = fma(y, in[19], in[38]);
+        const double h120 = fma(y, in[9], in[23]);
+        const double h121 = fma(x, h120, h119);
+        const double h122 = fma(z, in[9], in[24]);
+        const double h123 = fma(x, h122, h66);
+        const double h124 = fma(y, in[23], in[43]);
+        const double h125 = fma(y, h120, h124);
+        const double h126 = fma(y, h122, h114);
+        const double h127 = fma(z, in[24], in[45]);
+        const double h128 = fma(z, h122, h127);
+        out[0] = h2;
+        out[17] = h5;
+        out[34] = h8;
+        out[51] = h10;
+        out[68] = h12;
+        out[85] = h14;
+        out[102] = h17;
+        out[119] = h19;
+        out[136] = h21;
+        out[153] = h23;
+        out[170] = h25;
+        out[187] = h27;
+        out[204] = h30;
+        out[221] = h33;
+        out[238] = h35;
+        out[255] = h37;
+        out[272] = h38;
+        out[289] = h40;
+        out[306] = h43;
+        out[323] = h45;
+        out[340] = h47;
+        out[357] = h49;
+        out[374] = h51;
+        out[391] = h53;
+        out[408] = h56;
+        out[425] = h59;
+        out[442] = h61;
+        out[459] = h63;
+        out[476] = h65;
+        out[493] = h67;
+        out[510] = h70;
+        out[527] = h72;
+        out[544] = h74;
+        out[561] = h76;
+        out[578] = h77;
+        out[595] = h78;
+        out[612] = h81;
+        out[629] = h83;
+        out[646] = h85;
+        out[663] = h87;
+        out[680] = h89;
+        out[697] = h91;
+        out[714] = h94;
+        out[731] = h96;
+        out[748] = h98;
+        out[765] = h100;
+        out[782] = h101;
+        out[799] = h103;
+        out[816] = h106;
+        out[833] = h108;
+        out[850] = h110;
+        out[867] = h112;
+        out[884] = h113;
+        out[901] = h115;
+        out[918] = h118;
+        out[935] = h121;
+        out[952] = h123;
+        out[969] = h125;
+        out[986] = h126;
+        out[1003] = h128;
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[0], in[6]);
+        const double h1 = fma(y, in[0], in[7]);
+        const double h2 = fma(z, in[0], in[8]);
+        const double h3 = fma(x, in[1], in[7]);
+        const double h4 = fma(y, in[1], in[9]);
+        const double h5 = fma(z, in[1], in[11]);
+        const double h6 = fma(x, in[2], in[8]);
+        const double h7 = fma(y, in[2], in[11]);
+        const double h8 = fma(z, in[2], in[10]);
+        const double h9 = fma(x, in[3], in[9]);
+        const double h10 = fma(y, in[3], in[12]);
+        const double h11 = fma(z, in[3], in[13]);
+        const double h12 = fma(x, in[4], in[11]);
+        const double h13 = fma(y, in[4], in[13]);
+        const double h14 = fma(z, in[4], in[14]);
+        const double h15 = fma(x, in[5], in[10]);
+        const double h16 = fma(y, in[5], in[14]);
+        const double h17 = fma(z, in[5], in[15]);
+        out[0] = h0 * (nrm * 0.5773502691896258);
+        out[1] = h1 * (nrm * 0.5773502691896258);
+        out[2] = h2 * (nrm * 0.5773502691896258);
+        out[3] = h3 * (nrm * 1.0);
+        out[4] = h4 * (nrm * 1.0);
+        out[5] = h5 * (nrm * 1.0);
+        out[6] = h6 * (nrm * 1.0);
+        out[7] = h7 * (nrm * 1.0);
+        out[8] = h8 * (nrm * 1.0);
+        out[9] = h9 * (nrm * 0.5773502691896258);
+        out[10] = h10 * (nrm * 0.5773502691896258);
+        out[11] = h11 * (nrm * 0.5773502691896258);
+        out[12] = h12 * (nrm * 1.0);
+        out[13] = h13 * (nrm * 1.0);
+        out[14] = h14 * (nrm * 1.0);
+        out[15] = h15 * (nrm * 0.5773502691896258);
+        out[16] = h16 * (nrm * 0.5773502691896258);
+        out[17] = h17 * (nrm * 0.5773502691896258);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_fddp[736] = {
-    14, 269, 65549, 524, 65804, 131084, 15, 270, 65550, 525, 131085, 65805,
-    780, 66060, 131340, 196620, 1034, 1289, 66569, 1544, 66824, 132104, 1035, 1290,
-    66570, 1545, 132105, 66825, 1800, 67080, 132360, 197640, 262154, 262409, 327689, 262664,
-    327944, 393224, 262155, 262410, 327690, 262665, 393225, 327945, 262920, 328200, 393480, 458760,
-    2054, 2309, 67589, 2564, 67844, 133124, 2055, 2310, 67590, 2565, 133125, 67845,
-    2820, 68100, 133380, 198660, 524294, 524549, 589829, 524804, 590084, 655364, 524295, 524550,
-    589830, 524805, 655365, 590085, 525060, 590340, 655620, 720900, 263174, 263429, 328709, 263684,
-    328964, 394244, 263175, 263430, 328710, 263685, 394245, 328965, 263940, 329220, 394500, 459780,
-    3074, 3329, 68609, 3584, 68864, 134144, 3075, 3330, 68610, 3585, 134145, 68865,
-    3840, 69120, 134400, 199680, 264194, 264449, 329729, 264704, 329984, 395264, 264195, 264450,
-    329730, 264705, 395265, 329985, 264960, 330240, 395520, 460800, 525314, 525569, 590849, 525824,
-    591104, 656384, 525315, 525570, 590850, 525825, 656385, 591105, 526080, 591360, 656640, 721920,
-    786434, 786689, 851969, 786944, 852224, 917504, 786435, 786690, 851970, 786945, 917505, 852225,
-    787200, 852480, 917760, 983040, 18, 273, 65553, 528, 65808, 131088, 19, 274,
-    65554, 529, 131089, 65809, 784, 66064, 131344, 196624, 1038, 1293, 66573, 1548,
-    66828, 132108, 1039, 1294, 66574, 1549, 132109, 66829, 1804, 67084, 132364, 197644,
-    262158, 262413, 327693, 262668, 327948, 393228, 262159, 262414, 327694, 262669, 393229, 327949,
-    262924, 328204, 393484, 458764, 2058, 2313, 67593, 2568, 67848, 133128, 2059, 2314,
-    67594, 2569, 133129, 67849, 2824, 68104, 133384, 198664, 263178, 263433, 328713, 263688,
-    328968, 394248, 263179, 263434, 328714, 263689, 394249, 328969, 263944, 329224, 394504, 459784,
-    524298, 524553, 589833, 524808, 590088, 655368, 524299, 524554, 589834, 524809, 655369, 590089,
-    525064, 590344, 655624, 720904, 3078, 3333, 68613, 3588, 68868, 134148, 3079, 3334,
-    68614, 3589, 134149, 68869, 3844, 69124, 134404, 199684, 264198, 264453, 329733, 264708,
-    329988, 395268, 264199, 264454, 329734, 264709, 395269, 329989, 264964, 330244, 395524, 460804,
-    525318, 525573, 590853, 525828, 591108, 656388, 525319, 525574, 590854, 525829, 656389, 591109,
-    526084, 591364, 656644, 721924, 786438, 786693, 851973, 786948, 852228, 917508, 786439, 786694,
-    851974, 786949, 917509, 852229, 787204, 852484, 917764, 983044, 4098, 4353, 69633, 4608,
-    69888, 135168, 4099, 4354, 69634, 4609, 135169, 69889, 4864, 70144, 135424, 200704,
-    265218, 265473, 330753, 265728, 331008, 396288, 265219, 265474, 330754, 265729, 396289, 331009,
-    265984, 331264, 396544, 461824, 526338, 526593, 591873, 526848, 592128, 657408, 526339, 526594,
-    591874, 526849, 657409, 592129, 527104, 592384, 657664, 722944, 787458, 787713, 852993, 787968,
-    853248, 918528, 787459, 787714, 852994, 787969, 918529, 853249, 788224, 853504, 918784, 984064,
-    1048578, 1048833, 1114113, 1049088, 1114368, 1179648, 1048579, 1048834, 1114114, 1049089, 1179649, 1114369,
-    1049344, 1114624, 1179904, 1245184, 22, 277, 65557, 532, 65812, 131092, 23, 278,
-    65558, 533, 131093, 65813, 788, 66068, 131348, 196628, 1042, 1297, 66577, 1552,
-    66832, 132112, 1043, 1298, 66578, 1553, 132113, 66833, 1808, 67088, 132368, 197648,
-    262162, 262417, 327697, 262672, 327952, 393232, 262163, 262418, 327698, 262673, 393233, 327953,
-    262928, 328208, 393488, 458768, 2062, 2317, 67597, 2572, 67852, 133132, 2063, 2318,
-    67598, 2573, 133133, 67853, 2828, 68108, 133388, 198668, 263182, 263437, 328717, 263692,
-    328972, 394252, 263183, 263438, 328718, 263693, 394253, 328973, 263948, 329228, 394508, 459788,
-    524302, 524557, 589837, 524812, 590092, 655372, 524303, 524558, 589838, 524813, 655373, 590093,
-    525068, 590348, 655628, 720908, 3082, 3337, 68617, 3592, 68872, 134152, 3083, 3338,
-    68618, 3593, 134153, 68873, 3848, 69128, 134408, 199688, 264202, 264457, 329737, 264712,
-    329992, 395272, 264203, 264458, 329738, 264713, 395273, 329993, 264968, 330248, 395528, 460808,
-    525322, 525577, 590857, 525832, 591112, 656392, 525323, 525578, 590858, 525833, 656393, 591113,
-    526088, 591368, 656648, 721928, 786442, 786697, 851977, 786952, 852232, 917512, 786443, 786698,
-    851978, 786953, 917513, 852233, 787208, 852488, 917768, 983048, 4102, 4357, 69637, 4612,
-    69892, 135172, 4103, 4358, 69638, 4613, 135173, 69893, 4868, 70148, 135428, 200708,
-    265222, 265477, 330757, 265732, 331012, 396292, 265223, 265478, 330758, 265733, 396293, 331013,
-    265988, 331268, 396548, 461828, 526342, 526597, 591877, 526852, 592132, 657412, 526343, 526598,
-    591878, 526853, 657413, 592133, 527108, 592388, 657668, 722948, 787462, 787717, 852997, 787972,
-    853252, 918532, 787463, 787718, 852998, 787973, 918533, 853253, 788228, 853508, 918788, 984068,
-    1048582, 1048837, 1114117, 1049092, 1114372, 1179652, 1048583, 1048838, 1114118, 1049093, 1179653, 1114373,
-    1049348, 1114628, 1179908, 1245188, 5122, 5377, 70657, 5632, 70912, 136192, 5123, 5378,
-    70658, 5633, 136193, 70913, 5888, 71168, 136448, 201728, 266242, 266497, 331777, 266752,
-    332032, 397312, 266243, 266498, 331778, 266753, 397313, 332033, 267008, 332288, 397568, 462848,
-    527362, 527617, 592897, 527872, 593152, 658432, 527363, 527618, 592898, 527873, 658433, 593153,
-    528128, 593408, 658688, 723968, 788482, 788737, 854017, 788992, 854272, 919552, 788483, 788738,
-    854018, 788993, 919553, 854273, 789248, 854528, 919808, 985088, 1049602, 1049857, 1115137, 1050112,
-    1115392, 1180672, 1049603, 1049858, 1115138, 1050113, 1180673, 1115393, 1050368, 1115648, 1180928, 1246208,
-    1310722, 1310977, 1376257, 1311232, 1376512, 1441792, 1310723, 1310978, 1376258, 1311233, 1441793, 1376513,
-    1311488, 1376768, 1442048, 1507328,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_fddp[61] = {
-    0, 3, 7, 11, 14, 18, 21, 24, 28, 32, 35, 39,
-    42, 45, 49, 53, 56, 60, 63, 66, 70, 74, 77, 81,
-    84, 87, 91, 95, 98, 102, 105, 108, 112, 116, 119, 123,
-    126, 129, 133, 137, 140, 144, 147, 150, 154, 158, 161, 165,
-    168, 171, 175, 179, 182, 186, 189, 192, 196, 200, 203, 207,
-    210,
-};
-__device__ const uint32_t kBraTerm_fddp[210] = {
-    66560, 131338, 65561, 66816, 65803, 66058, 65562, 67072, 65804, 66314, 65563, 67328,
-    131595, 65564, 67584, 66060, 66315, 65565, 67840, 131852, 65566, 66561, 131339, 65562,
-    66817, 65805, 66059, 65564, 67073, 65806, 66315, 65565, 67329, 131597, 65567, 67585,
-    66062, 66317, 65568, 67841, 131854, 65569, 66562, 131340, 65563, 66818, 65806, 66060,
-    65565, 67074, 65807, 66316, 65566, 67330, 131598, 65568, 67586, 66063, 66318, 65569,
-    67842, 131855, 65570, 66563, 131341, 65564, 66819, 65808, 66061, 65567, 67075, 65809,
-    66317, 65568, 67331, 131600, 65571, 67587, 66065, 66320, 65572, 67843, 131857, 65573,
-    66564, 131343, 65566, 66820, 65810, 66063, 65569, 67076, 65811, 66319, 65570, 67332,
-    131602, 65573, 67588, 66067, 66322, 65574, 67844, 131859, 65575, 66565, 131342, 65565,
-    66821, 65809, 66062, 65568, 67077, 65810, 66318, 65569, 67333, 131601, 65572, 67589,
-    66066, 66321, 65573, 67845, 131858, 65574, 66566, 131344, 65567, 66822, 65812, 66064,
-    65571, 67078, 65813, 66320, 65572, 67334, 131604, 65576, 67590, 66069, 66324, 65577,
-    67846, 131861, 65578, 66567, 131345, 65568, 66823, 65813, 66065, 65572, 67079, 65814,
-    66321, 65573, 67335, 131605, 65577, 67591, 66070, 66325, 65578, 67847, 131862, 65579,
-    66568, 131346, 65569, 66824, 65814, 66066, 65573, 67080, 65815, 66322, 65574, 67336,
-    131606, 65578, 67592, 66071, 66326, 65579, 67848, 131863, 65580, 66569, 131347, 65570,
-    66825, 65815, 66067, 65574, 67081, 65816, 66323, 65575, 67337, 131607, 65579, 67593,
-    66072, 66327, 65580, 67849, 131864, 65581,
-};
-__device__ const uint16_t kKetOff_fddp[19] = {
-    0, 2, 4, 6, 8, 10, 12, 14, 16, 18, 20, 22,
-    24, 26, 28, 30, 32, 34, 36,
-};
-__device__ const uint32_t kKetTerm_fddp[36] = {
-    65792, 65542, 66048, 65543, 66304, 65544, 65793, 65543, 66049, 65545, 66305, 65547,
-    65794, 65544, 66050, 65547, 66306, 65546, 65795, 65545, 66051, 65548, 66307, 65549,
-    65796, 65547, 66052, 65549, 66308, 65550, 65797, 65546, 66053, 65550, 66309, 65551,
-};
 __device__ const double kNormAB_fddp[60] = {
     0.14907119849998599, 0.2581988897471611, 0.2581988897471611, 0.14907119849998599,
     0.2581988897471611, 0.14907119849998599, 0.3333333333333334, 0.5773502691896258,
@@ -188,21 +315,12 @@ __device__ const double kNormAB_fddp[60] = {
     0.5773502691896258, 0.3333333333333334, 0.14907119849998599, 0.2581988897471611,
     0.2581988897471611, 0.14907119849998599, 0.2581988897471611, 0.14907119849998599,
 };
-__device__ const double kNormCD_fddp[18] = {
-    0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 1.0,
-    1.0, 1.0, 1.0, 1.0,
-    1.0, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
-    1.0, 1.0, 1.0, 0.5773502691896258,
-    0.5773502691896258, 0.5773502691896258,
-};
-
 
 // column components cx | cy << 4 | cz << 8
 __device__ const uint16_t kCol_fddp[16] = { 2, 17, 257, 32, 272, 512, 3, 18, 258, 33, 513, 273, 48, 288, 528, 768 };
 
 __device__ __forceinline__ RysClassTabs tabs_fddp() {
-    return RysClassTabs{kBlk_fddp, kBraOff_fddp, kBraTerm_fddp, kKetOff_fddp, kKetTerm_fddp,
-                        kNormAB_fddp, kNormCD_fddp, kCol_fddp};
+    return RysClassTabs{kNormAB_fddp, kCol_fddp};
 }
 
 template <int MIXED>
@@ -215,8 +333,8 @@ static void rys_prepare_fddp() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_fddp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 70400);
-        cudaFuncSetAttribute(rys_queue_fddp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 70400);
+        cudaFuncSetAttribute(rys_queue_fddp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 69120);
+        cudaFuncSetAttribute(rys_queue_fddp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 69120);
 
         done[dev] = true;
     }
@@ -228,16 +346,16 @@ void launch_rys_fddp(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_fddp();
     constexpr int ng = 128 / C_fddp::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_fddp<1><<<grid, 128, 70400, s>>>(Q, R);
-    else rys_queue_fddp<0><<<grid, 128, 70400, s>>>(Q, R);
+    if (mixed) rys_queue_fddp<1><<<grid, 128, 69120, s>>>(Q, R);
+    else rys_queue_fddp<0><<<grid, 128, 69120, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_fddp(int mixed) {
     rys_prepare_fddp();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fddp<1>, 128, 70400);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fddp<0>, 128, 70400);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fddp<1>, 128, 69120);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fddp<0>, 128, 69120);
     return n;
 }
 

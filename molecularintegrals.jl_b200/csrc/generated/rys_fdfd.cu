@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (fd|fd).  Do not edit.
-// roots 6, block 46 x 46, outputs 60 x 60, group 64 threads,
-// 9 primitive quartets per batch, 1 slot(s), 1 accumulators per thread, 93952 B shared per block, column mode.
+// roots 6, block 46 x 46, outputs 60 x 60, group 64 threads, 1 ket pairs a round,
+// 9 primitive quartets per ket pair and batch, 103680 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,11 +11,10 @@ struct C_fdfd {
     static constexpr int NA = 46, NC = 46, NBLK = 2116;
     static constexpr int NB = 6, ND = 6;
     static constexpr int NAB = 60, NCD = 60;
-    static constexpr int G = 64, NPB = 9, NSLOT = 1, ACC = 1;
-    static constexpr int S = 36;
-    static constexpr int SMEM_GROUP = 5872;
-    static constexpr bool COL = true;
-    // stage 2, column mode: acc[row] += x[ax] y[ay] z[az] for the column's table columns
+    static constexpr int G = 64, W = 1, H = 1, PB = 9;
+    static constexpr int S = 36, SI = 109, NCP = 47, NCDP = 61;
+    static constexpr int SMEM_GROUP = 6480;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
     __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
         acc[0] = fma(x[3] * y[0], z[0], acc[0]);
@@ -65,246 +64,393 @@ struct C_fdfd {
         acc[44] = fma(x[0] * y[1], z[4], acc[44]);
         acc[45] = fma(x[0] * y[0], z[5], acc[45]);
     }
-    static constexpr int NCOLS = 46;
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[10], in[25]);
+        const double h1 = fma(x, in[0], in[10]);
+        const double h2 = fma(x, h1, h0);
+        const double h3 = fma(y, in[10], in[26]);
+        const double h4 = fma(y, in[0], in[11]);
+        const double h5 = fma(x, h4, h3);
+        const double h6 = fma(z, in[10], in[27]);
+        const double h7 = fma(z, in[0], in[12]);
+        const double h8 = fma(x, h7, h6);
+        const double h9 = fma(y, in[11], in[28]);
+        const double h10 = fma(y, h4, h9);
+        const double h11 = fma(z, in[11], in[29]);
+        const double h12 = fma(y, h7, h11);
+        const double h13 = fma(z, in[12], in[30]);
+        const double h14 = fma(z, h7, h13);
+        const double h15 = fma(x, in[11], in[26]);
+        const double h16 = fma(x, in[1], in[11]);
+        const double h17 = fma(x, h16, h15);
+        const double h18 = fma(y, in[1], in[13]);
+        const double h19 = fma(x, h18, h9);
+        const double h20 = fma(z, in[1], in[14]);
+        const double h21 = fma(x, h20, h11);
+        const double h22 = fma(y, in[13], in[31]);
+        const double h23 = fma(y, h18, h22);
+        const double h24 = fma(z, in[13], in[32]);
+        const double h25 = fma(y, h20, h24);
+        const double h26 = fma(z, in[14], in[33]);
+        const double h27 = fma(z, h20, h26);
+        const double h28 = fma(x, in[12], in[27]);
+        const double h29 = fma(x, in[2], in[12]);
+        const double h30 = fma(x, h29, h28);
+        const double h31 = fma(y, in[12], in[29]);
+        const double h32 = fma(y, in[2], in[14]);
+        const double h33 = fma(x, h32, h31);
+        const double h34 = fma(z, in[2], in[15]);
+        const double h35 = fma(x, h34, h13);
+        const double h36 = fma(y, in[14], in[32]);
+        const double h37 = fma(y, h32, h36);
+        const double h38 = fma(y, h34, h26);
+        const double h39 = fma(z, in[15], in[34]);
+        const double h40 = fma(z, h34, h39);
+        const double h41 = fma(x, in[13], in[28]);
+        const double h42 = fma(x, in[3], in[13]);
+        const double h43 = fma(x, h42, h41);
+        const double h44 = fma(y, in[3], in[16]);
+        const double h45 = fma(x, h44, h22);
+        const double h46 = fma(z, in[3], in[17]);
+        const double h47 = fma(x, h46, h24);
+        const double h48 = fma(y, in[16], in[35]);
+        const double h49 = fma(y, h44, h48);
+        const double h50 = fma(z, in[16], in[36]);
+        const double h51 = fma(y, h46, h50);
+        const double h52 = fma(z, in[17], in[37]);
+        const double h53 = fma(z, h46, h52);
+        const double h54 = fma(x, in[15], in[30]);
+        const double h55 = fma(x, in[4], in[15]);
+        const double h56 = fma(x, h55, h54);
+        const double h57 = fma(y, in[15], in[33]);
+        const double h58 = fma(y, in[4], in[18]);
+        const double h59 = fma(x, h58, h57);
+        const double h60 = fma(z, in[4], in[19]);
+        const double h61 = fma(x, h60, h39);
+        const double h62 = fma(y, in[18], in[37]);
+        const double h63 = fma(y, h58, h62);
+        const double h64 = fma(z, in[18], in[38]);
+        const double h65 = fma(y, h60, h64);
+        const double h66 = fma(z, in[19], in[39]);
+        const double h67 = fma(z, h60, h66);
+        const double h68 = fma(x, in[14], in[29]);
+        const double h69 = fma(x, in[5], in[14]);
+        const double h70 = fma(x, h69, h68);
+        const double h71 = fma(y, in[5], in[17]);
+        const double h72 = fma(x, h71, h36);
+        const double h73 = fma(z, in[5], in[18]);
+        const double h74 = fma(x, h73, h26);
+        const double h75 = fma(y, in[17], in[36]);
+        const double h76 = fma(y, h71, h75);
+        const double h77 = fma(y, h73, h52);
+        const double h78 = fma(z, h73, h64);
+        const double h79 = fma(x, in[16], in[31]);
+        const double h80 = fma(x, in[6], in[16]);
+        const double h81 = fma(x, h80, h79);
+        const double h82 = fma(y, in[6], in[20]);
+        const double h83 = fma(x, h82, h48);
+        const double h84 = fma(z, in[6], in[21]);
+        const double h85 = fma(x, h84, h50);
+        const double h86 = fma(y, in[20], in[40]);
+        const double h87 = fma(y, h82, h86);
+        const double h88 = fma(z, in[20], in[41]);
+        const double h89 = fma(y, h84, h88);
+        const double h90 = fma(z, in[21], in[42]);
+        const double h91 = fma(z, h84, h90);
+        const double h92 = fma(x, in[17], in[32]);
+        const double h93 = fma(x, in[7], in[17]);
+        const double h94 = fma(x, h93, h92);
+        const double h95 = fma(y, in[7], in[21]);
+        const double h96 = fma(x, h95, h75);
+        const double h97 = fma(z, in[7], in[22]);
+        const double h98 = fma(x, h97, h52);
+        const double h99 = fma(y, in[21], in[41]);
+        const double h100 = fma(y, h95, h99);
+        const double h101 = fma(y, h97, h90);
+        const double h102 = fma(z, in[22], in[43]);
+        const double h103 = fma(z, h97, h102);
+        const double h104 = fma(x, in[18], in[33]);
+        const double h105 = fma(x, in[8], in[18]);
+        const double h106 = fma(x, h105, h104);
+        const double h107 = fma(y, in[8], in[22]);
+        const double h108 = fma(x, h107, h62);
+        const double h109 = fma(z, in[8], in[23]);
+        const double h110 = fma(x, h109, h64);
+        const double h111 = fma(y, in[22], in[42]);
+        const double h112 = fma(y, h107, h111);
+        const double h113 = fma(y, h109, h102);
+        const double h114 = fma(z, in[23], in[44]);
+        const double h115 = fma(z, h109, h114);
+        const double h116 = fma(x, in[19], in[34]);
+        const double h117 = fma(x, in[9], in[19]);
+        const double h118 = fma(x, h117, h116);
+        const double h119 = fma(y, in[19], in[38]);
+        const double h120 = fma(y, in[9], in[23]);
+        const double h121 = fma(x, h120, h119);
+        const double h122 = fma(z, in[9], in[24]);
+        const double h123 = fma(x, h122, h66);
+        const double h124 = fma(y, in[23], in[43]);
+        const double h125 = fma(y, h120, h124);
+        const double h126 = fma(y, h122, h114);
+        const double h127 = fma(z, in[24], in[45]);
+        const double h128 = fma(z, h122, h127);
+        out[0] = h2;
+        out[47] = h5;
+        out[94] = h8;
+        out[141] = h10;
+        out[188] = h12;
+        out[235] = h14;
+        out[282] = h17;
+        out[329] = h19;
+        out[376] = h21;
+        out[423] = h23;
+        out[470] = h25;
+        out[517] = h27;
+        out[564] = h30;
+        out[611] = h33;
+        out[658] = h35;
+        out[705] = h37;
+        out[752] = h38;
+        out[799] = h40;
+        out[846] = h43;
+        out[893] = h45;
+        out[940] = h47;
+        out[987] = h49;
+        out[1034] = h51;
+        out[1081] = h53;
+        out[1128] = h56;
+        out[1175] = h59;
+        out[1222] = h61;
+        out[1269] = h63;
+        out[1316] = h65;
+        out[1363] = h67;
+        out[1410] = h70;
+        out[1457] = h72;
+        out[1504] = h74;
+        out[1551] = h76;
+        out[1598] = h77;
+        out[1645] = h78;
+        out[1692] = h81;
+        out[1739] = h83;
+        out[1786] = h85;
+        out[1833] = h87;
+        out[1880] = h89;
+        out[1927] = h91;
+        out[1974] = h94;
+        out[2021] = h96;
+        out[2068] = h98;
+        out[2115] = h100;
+        out[2162] = h101;
+        out[2209] = h103;
+        out[2256] = h106;
+        out[2303] = h108;
+        out[2350] = h110;
+        out[2397] = h112;
+        out[2444] = h113;
+        out[2491] = h115;
+        out[2538] = h118;
+        out[2585] = h121;
+        out[2632] = h123;
+        out[2679] = h125;
+        out[2726] = h126;
+        out[2773] = h128;
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[10], in[25]);
+        const double h1 = fma(x, in[0], in[10]);
+        const double h2 = fma(x, h1, h0);
+        const double h3 = fma(y, in[10], in[26]);
+        const double h4 = fma(y, in[0], in[11]);
+        const double h5 = fma(x, h4, h3);
+        const double h6 = fma(z, in[10], in[27]);
+        const double h7 = fma(z, in[0], in[12]);
+        const double h8 = fma(x, h7, h6);
+        const double h9 = fma(y, in[11], in[28]);
+        const double h10 = fma(y, h4, h9);
+        const double h11 = fma(z, in[11], in[29]);
+        const double h12 = fma(y, h7, h11);
+        const double h13 = fma(z, in[12], in[30]);
+        const double h14 = fma(z, h7, h13);
+        const double h15 = fma(x, in[11], in[26]);
+        const double h16 = fma(x, in[1], in[11]);
+        const double h17 = fma(x, h16, h15);
+        const double h18 = fma(y, in[1], in[13]);
+        const double h19 = fma(x, h18, h9);
+        const double h20 = fma(z, in[1], in[14]);
+        const double h21 = fma(x, h20, h11);
+        const double h22 = fma(y, in[13], in[31]);
+        const double h23 = fma(y, h18, h22);
+        const double h24 = fma(z, in[13], in[32]);
+        const double h25 = fma(y, h20, h24);
+        const double h26 = fma(z, in[14], in[33]);
+        const double h27 = fma(z, h20, h26);
+        const double h28 = fma(x, in[12], in[27]);
+        const double h29 = fma(x, in[2], in[12]);
+        const double h30 = fma(x, h29, h28);
+        const double h31 = fma(y, in[12], in[29]);
+        const double h32 = fma(y, in[2], in[14]);
+        const double h33 = fma(x, h32, h31);
+        const double h34 = fma(z, in[2], in[15]);
+        const double h35 = fma(x, h34, h13);
+        const double h36 = fma(y, in[14], in[32]);
+        const double h37 = fma(y, h32, h36);
+        const double h38 = fma(y, h34, h26);
+        const double h39 = fma(z, in[15], in[34]);
+        const double h40 = fma(z, h34, h39);
+        const double h41 = fma(x, in[13], in[28]);
+        const double h42 = fma(x, in[3], in[13]);
+        const double h43 = fma(x, h42, h41);
+        const double h44 = fma(y, in[3], in[16]);
+        const double h45 = fma(x, h44, h22);
+        const double h46 = fma(z, in[3], in[17]);
+        const double h47 = fma(x, h46, h24);
+        const double h48 = fma(y, in[16], in[35]);
+        const double h49 = fma(y, h44, h48);
+        const double h50 = fma(z, in[16], in[36]);
+        const double h51 = fma(y, h46, h50);
+        const double h52 = fma(z, in[17], in[37]);
+        const double h53 = fma(z, h46, h52);
+        const double h54 = fma(x, in[15], in[30]);
+        const double h55 = fma(x, in[4], in[15]);
+        const double h56 = fma(x, h55, h54);
+        const double h57 = fma(y, in[15], in[33]);
+        const double h58 = fma(y, in[4], in[18]);
+        const double h59 = fma(x, h58, h57);
+        const double h60 = fma(z, in[4], in[19]);
+        const double h61 = fma(x, h60, h39);
+        const double h62 = fma(y, in[18], in[37]);
+        const double h63 = fma(y, h58, h62);
+        const double h64 = fma(z, in[18], in[38]);
+        const double h65 = fma(y, h60, h64);
+        const double h66 = fma(z, in[19], in[39]);
+        const double h67 = fma(z, h60, h66);
+        const double h68 = fma(x, in[14], in[29]);
+        const double h69 = fma(x, in[5], in[14]);
+        const double h70 = fma(x, h69, h68);
+        const double h71 = fma(y, in[5], in[17]);
+        const double h72 = fma(x, h71, h36);
+        const double h73 = fma(z, in[5], in[18]);
+        const double h74 = fma(x, h73, h26);
+        const double h75 = fma(y, in[17], in[36]);
+        const double h76 = fma(y, h71, h75);
+        const double h77 = fma(y, h73, h52);
+        const double h78 = fma(z, h73, h64);
+        const double h79 = fma(x, in[16], in[31]);
+        const double h80 = fma(x, in[6], in[16]);
+        const double h81 = fma(x, h80, h79);
+        const double h82 = fma(y, in[6], in[20]);
+        const double h83 = fma(x, h82, h48);
+        const double h84 = fma(z, in[6], in[21]);
+        const double h85 = fma(x, h84, h50);
+        const double h86 = fma(y, in[20], in[40]);
+        const double h87 = fma(y, h82, h86);
+        const double h88 = fma(z, in[20], in[41]);
+        const double h89 = fma(y, h84, h88);
+        const double h90 = fma(z, in[21], in[42]);
+        const double h91 = fma(z, h84, h90);
+        const double h92 = fma(x, in[17], in[32]);
+        const double h93 = fma(x, in[7], in[17]);
+        const double h94 = fma(x, h93, h92);
+        const double h95 = fma(y, in[7], in[21]);
+        const double h96 = fma(x, h95, h75);
+        const double h97 = fma(z, in[7], in[22]);
+        const double h98 = fma(x, h97, h52);
+        const double h99 = fma(y, in[21], in[41]);
+        const double h100 = fma(y, h95, h99);
+        const double h101 = fma(y, h97, h90);
+        const double h102 = fma(z, in[22], in[43]);
+        const double h103 = fma(z, h97, h102);
+        const double h104 = fma(x, in[18], in[33]);
+        const double h105 = fma(x, in[8], in[18]);
+        const double h106 = fma(x, h105, h104);
+        const double h107 = fma(y, in[8], in[22]);
+        const double h108 = fma(x, h107, h62);
+        const double h109 = fma(z, in[8], in[23]);
+        const double h110 = fma(x, h109, h64);
+        const double h111 = fma(y, in[22], in[42]);
+        const double h112 = fma(y, h107, h111);
+        const double h113 = fma(y, h109, h102);
+        const double h114 = fma(z, in[23], in[44]);
+        const double h115 = fma(z, h109, h114);
+        const double h116 = fma(x, in[19], in[34]);
+        const double h117 = fma(x, in[9], in[19]);
+        const double h118 = fma(x, h117, h116);
+        const double h119 = fma(y, in[19], in[38]);
+        const double h120 = fma(y, in[9], in[23]);
+        const double h121 = fma(x, h120, h119);
+        const double h122 = fma(z, in[9], in[24]);
+        const double h123 = fma(x, h122, h66);
+        const double h124 = fma(y, in[23], in[43]);
+        const double h125 = fma(y, h120, h124);
+        const double h126 = fma(y, h122, h114);
+        const double h127 = fma(z, in[24], in[45]);
+        const double h128 = fma(z, h122, h127);
+        out[0] = h2 * (nrm * 0.14907119849998599);
+        out[1] = h5 * (nrm * 0.2581988897471611);
+        out[2] = h8 * (nrm * 0.2581988897471611);
+        out[3] = h10 * (nrm * 0.14907119849998599);
+        out[4] = h12 * (nrm * 0.2581988897471611);
+        out[5] = h14 * (nrm * 0.14907119849998599);
+        out[6] = h17 * (nrm * 0.3333333333333334);
+        out[7] = h19 * (nrm * 0.5773502691896258);
+        out[8] = h21 * (nrm * 0.5773502691896258);
+        out[9] = h23 * (nrm * 0.3333333333333334);
+        out[10] = h25 * (nrm * 0.5773502691896258);
+        out[11] = h27 * (nrm * 0.3333333333333334);
+        out[12] = h30 * (nrm * 0.3333333333333334);
+        out[13] = h33 * (nrm * 0.5773502691896258);
+        out[14] = h35 * (nrm * 0.5773502691896258);
+        out[15] = h37 * (nrm * 0.3333333333333334);
+        out[16] = h38 * (nrm * 0.5773502691896258);
+        out[17] = h40 * (nrm * 0.3333333333333334);
+        out[18] = h43 * (nrm * 0.3333333333333334);
+        out[19] = h45 * (nrm * 0.5773502691896258);
+        out[20] = h47 * (nrm * 0.5773502691896258);
+        out[21] = h49 * (nrm * 0.3333333333333334);
+        out[22] = h51 * (nrm * 0.5773502691896258);
+        out[23] = h53 * (nrm * 0.3333333333333334);
+        out[24] = h56 * (nrm * 0.3333333333333334);
+        out[25] = h59 * (nrm * 0.5773502691896258);
+        out[26] = h61 * (nrm * 0.5773502691896258);
+        out[27] = h63 * (nrm * 0.3333333333333334);
+        out[28] = h65 * (nrm * 0.5773502691896258);
+        out[29] = h67 * (nrm * 0.3333333333333334);
+        out[30] = h70 * (nrm * 0.5773502691896258);
+        out[31] = h72 * (nrm * 1.0);
+        out[32] = h74 * (nrm * 1.0);
+        out[33] = h76 * (nrm * 0.5773502691896258);
+        out[34] = h77 * (nrm * 1.0);
+        out[35] = h78 * (nrm * 0.5773502691896258);
+        out[36] = h81 * (nrm * 0.14907119849998599);
+        out[37] = h83 * (nrm * 0.2581988897471611);
+        out[38] = h85 * (nrm * 0.2581988897471611);
+        out[39] = h87 * (nrm * 0.14907119849998599);
+        out[40] = h89 * (nrm * 0.2581988897471611);
+        out[41] = h91 * (nrm * 0.14907119849998599);
+        out[42] = h94 * (nrm * 0.3333333333333334);
+        out[43] = h96 * (nrm * 0.5773502691896258);
+        out[44] = h98 * (nrm * 0.5773502691896258);
+        out[45] = h100 * (nrm * 0.3333333333333334);
+        out[46] = h101 * (nrm * 0.5773502691896258);
+        out[47] = h103 * (nrm * 0.3333333333333334);
+        out[48] = h106 * (nrm * 0.3333333333333334);
+        out[49] = h108 * (nrm * 0.5773502691896258);
+        out[50] = h110 * (nrm * 0.5773502691896258);
+        out[51] = h112 * (nrm * 0.3333333333333334);
+        out[52] = h113 * (nrm * 0.5773502691896258);
+        out[53] = h115 * (nrm * 0.3333333333333334);
+        out[54] = h118 * (nrm * 0.14907119849998599);
+        out[55] = h121 * (nrm * 0.2581988897471611);
+        out[56] = h123 * (nrm * 0.2581988897471611);
+        out[57] = h125 * (nrm * 0.14907119849998599);
+        out[58] = h126 * (nrm * 0.2581988897471611);
+        out[59] = h128 * (nrm * 0.14907119849998599);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_fdfd[2116] = {
-    21, 276, 65556, 531, 131091, 65811, 786, 66066, 131346, 196626, 22, 277,
-    65557, 532, 65812, 131092, 787, 66067, 131347, 196627, 1042, 66322, 131602, 196882,
-    262162, 23, 278, 65558, 533, 65813, 131093, 788, 66068, 131348, 196628, 1043,
-    66323, 131603, 196883, 262163, 1298, 66578, 131858, 197138, 262418, 327698, 1551, 1806,
-    67086, 2061, 132621, 67341, 2316, 67596, 132876, 198156, 1552, 1807, 67087, 2062,
-    67342, 132622, 2317, 67597, 132877, 198157, 2572, 67852, 133132, 198412, 263692, 1553,
-    1808, 67088, 2063, 67343, 132623, 2318, 67598, 132878, 198158, 2573, 67853, 133133,
-    198413, 263693, 2828, 68108, 133388, 198668, 263948, 329228, 393231, 393486, 458766, 393741,
-    524301, 459021, 393996, 459276, 524556, 589836, 393232, 393487, 458767, 393742, 459022, 524302,
-    393997, 459277, 524557, 589837, 394252, 459532, 524812, 590092, 655372, 393233, 393488, 458768,
-    393743, 459023, 524303, 393998, 459278, 524558, 589838, 394253, 459533, 524813, 590093, 655373,
-    394508, 459788, 525068, 590348, 655628, 720908, 3081, 3336, 68616, 3591, 134151, 68871,
-    3846, 69126, 134406, 199686, 3082, 3337, 68617, 3592, 68872, 134152, 3847, 69127,
-    134407, 199687, 4102, 69382, 134662, 199942, 265222, 3083, 3338, 68618, 3593, 68873,
-    134153, 3848, 69128, 134408, 199688, 4103, 69383, 134663, 199943, 265223, 4358, 69638,
-    134918, 200198, 265478, 330758, 786441, 786696, 851976, 786951, 917511, 852231, 787206, 852486,
-    917766, 983046, 786442, 786697, 851977, 786952, 852232, 917512, 787207, 852487, 917767, 983047,
-    787462, 852742, 918022, 983302, 1048582, 786443, 786698, 851978, 786953, 852233, 917513, 787208,
-    852488, 917768, 983048, 787463, 852743, 918023, 983303, 1048583, 787718, 852998, 918278, 983558,
-    1048838, 1114118, 394761, 395016, 460296, 395271, 525831, 460551, 395526, 460806, 526086, 591366,
-    394762, 395017, 460297, 395272, 460552, 525832, 395527, 460807, 526087, 591367, 395782, 461062,
-    526342, 591622, 656902, 394763, 395018, 460298, 395273, 460553, 525833, 395528, 460808, 526088,
-    591368, 395783, 461063, 526343, 591623, 656903, 396038, 461318, 526598, 591878, 657158, 722438,
-    4611, 4866, 70146, 5121, 135681, 70401, 5376, 70656, 135936, 201216, 4612, 4867,
-    70147, 5122, 70402, 135682, 5377, 70657, 135937, 201217, 5632, 70912, 136192, 201472,
-    266752, 4613, 4868, 70148, 5123, 70403, 135683, 5378, 70658, 135938, 201218, 5633,
-    70913, 136193, 201473, 266753, 5888, 71168, 136448, 201728, 267008, 332288, 396291, 396546,
-    461826, 396801, 527361, 462081, 397056, 462336, 527616, 592896, 396292, 396547, 461827, 396802,
-    462082, 527362, 397057, 462337, 527617, 592897, 397312, 462592, 527872, 593152, 658432, 396293,
-    396548, 461828, 396803, 462083, 527363, 397058, 462338, 527618, 592898, 397313, 462593, 527873,
-    593153, 658433, 397568, 462848, 528128, 593408, 658688, 723968, 787971, 788226, 853506, 788481,
-    919041, 853761, 788736, 854016, 919296, 984576, 787972, 788227, 853507, 788482, 853762, 919042,
-    788737, 854017, 919297, 984577, 788992, 854272, 919552, 984832, 1050112, 787973, 788228, 853508,
-    788483, 853763, 919043, 788738, 854018, 919298, 984578, 788993, 854273, 919553, 984833, 1050113,
-    789248, 854528, 919808, 985088, 1050368, 1115648, 1179651, 1179906, 1245186, 1180161, 1310721, 1245441,
-    1180416, 1245696, 1310976, 1376256, 1179652, 1179907, 1245187, 1180162, 1245442, 1310722, 1180417, 1245697,
-    1310977, 1376257, 1180672, 1245952, 1311232, 1376512, 1441792, 1179653, 1179908, 1245188, 1180163, 1245443,
-    1310723, 1180418, 1245698, 1310978, 1376258, 1180673, 1245953, 1311233, 1376513, 1441793, 1180928, 1246208,
-    1311488, 1376768, 1442048, 1507328, 27, 282, 65562, 537, 131097, 65817, 792, 66072,
-    131352, 196632, 28, 283, 65563, 538, 65818, 131098, 793, 66073, 131353, 196633,
-    1048, 66328, 131608, 196888, 262168, 29, 284, 65564, 539, 65819, 131099, 794,
-    66074, 131354, 196634, 1049, 66329, 131609, 196889, 262169, 1304, 66584, 131864, 197144,
-    262424, 327704, 1557, 1812, 67092, 2067, 132627, 67347, 2322, 67602, 132882, 198162,
-    1558, 1813, 67093, 2068, 67348, 132628, 2323, 67603, 132883, 198163, 2578, 67858,
-    133138, 198418, 263698, 1559, 1814, 67094, 2069, 67349, 132629, 2324, 67604, 132884,
-    198164, 2579, 67859, 133139, 198419, 263699, 2834, 68114, 133394, 198674, 263954, 329234,
-    393237, 393492, 458772, 393747, 524307, 459027, 394002, 459282, 524562, 589842, 393238, 393493,
-    458773, 393748, 459028, 524308, 394003, 459283, 524563, 589843, 394258, 459538, 524818, 590098,
-    655378, 393239, 393494, 458774, 393749, 459029, 524309, 394004, 459284, 524564, 589844, 394259,
-    459539, 524819, 590099, 655379, 394514, 459794, 525074, 590354, 655634, 720914, 3087, 3342,
-    68622, 3597, 134157, 68877, 3852, 69132, 134412, 199692, 3088, 3343, 68623, 3598,
-    68878, 134158, 3853, 69133, 134413, 199693, 4108, 69388, 134668, 199948, 265228, 3089,
-    3344, 68624, 3599, 68879, 134159, 3854, 69134, 134414, 199694, 4109, 69389, 134669,
-    199949, 265229, 4364, 69644, 134924, 200204, 265484, 330764, 394767, 395022, 460302, 395277,
-    525837, 460557, 395532, 460812, 526092, 591372, 394768, 395023, 460303, 395278, 460558, 525838,
-    395533, 460813, 526093, 591373, 395788, 461068, 526348, 591628, 656908, 394769, 395024, 460304,
-    395279, 460559, 525839, 395534, 460814, 526094, 591374, 395789, 461069, 526349, 591629, 656909,
-    396044, 461324, 526604, 591884, 657164, 722444, 786447, 786702, 851982, 786957, 917517, 852237,
-    787212, 852492, 917772, 983052, 786448, 786703, 851983, 786958, 852238, 917518, 787213, 852493,
-    917773, 983053, 787468, 852748, 918028, 983308, 1048588, 786449, 786704, 851984, 786959, 852239,
-    917519, 787214, 852494, 917774, 983054, 787469, 852749, 918029, 983309, 1048589, 787724, 853004,
-    918284, 983564, 1048844, 1114124, 4617, 4872, 70152, 5127, 135687, 70407, 5382, 70662,
-    135942, 201222, 4618, 4873, 70153, 5128, 70408, 135688, 5383, 70663, 135943, 201223,
-    5638, 70918, 136198, 201478, 266758, 4619, 4874, 70154, 5129, 70409, 135689, 5384,
-    70664, 135944, 201224, 5639, 70919, 136199, 201479, 266759, 5894, 71174, 136454, 201734,
-    267014, 332294, 396297, 396552, 461832, 396807, 527367, 462087, 397062, 462342, 527622, 592902,
-    396298, 396553, 461833, 396808, 462088, 527368, 397063, 462343, 527623, 592903, 397318, 462598,
-    527878, 593158, 658438, 396299, 396554, 461834, 396809, 462089, 527369, 397064, 462344, 527624,
-    592904, 397319, 462599, 527879, 593159, 658439, 397574, 462854, 528134, 593414, 658694, 723974,
-    787977, 788232, 853512, 788487, 919047, 853767, 788742, 854022, 919302, 984582, 787978, 788233,
-    853513, 788488, 853768, 919048, 788743, 854023, 919303, 984583, 788998, 854278, 919558, 984838,
-    1050118, 787979, 788234, 853514, 788489, 853769, 919049, 788744, 854024, 919304, 984584, 788999,
-    854279, 919559, 984839, 1050119, 789254, 854534, 919814, 985094, 1050374, 1115654, 1179657, 1179912,
-    1245192, 1180167, 1310727, 1245447, 1180422, 1245702, 1310982, 1376262, 1179658, 1179913, 1245193, 1180168,
-    1245448, 1310728, 1180423, 1245703, 1310983, 1376263, 1180678, 1245958, 1311238, 1376518, 1441798, 1179659,
-    1179914, 1245194, 1180169, 1245449, 1310729, 1180424, 1245704, 1310984, 1376264, 1180679, 1245959, 1311239,
-    1376519, 1441799, 1180934, 1246214, 1311494, 1376774, 1442054, 1507334, 6147, 6402, 71682, 6657,
-    137217, 71937, 6912, 72192, 137472, 202752, 6148, 6403, 71683, 6658, 71938, 137218,
-    6913, 72193, 137473, 202753, 7168, 72448, 137728, 203008, 268288, 6149, 6404, 71684,
-    6659, 71939, 137219, 6914, 72194, 137474, 202754, 7169, 72449, 137729, 203009, 268289,
-    7424, 72704, 137984, 203264, 268544, 333824, 397827, 398082, 463362, 398337, 528897, 463617,
-    398592, 463872, 529152, 594432, 397828, 398083, 463363, 398338, 463618, 528898, 398593, 463873,
-    529153, 594433, 398848, 464128, 529408, 594688, 659968, 397829, 398084, 463364, 398339, 463619,
-    528899, 398594, 463874, 529154, 594434, 398849, 464129, 529409, 594689, 659969, 399104, 464384,
-    529664, 594944, 660224, 725504, 789507, 789762, 855042, 790017, 920577, 855297, 790272, 855552,
-    920832, 986112, 789508, 789763, 855043, 790018, 855298, 920578, 790273, 855553, 920833, 986113,
-    790528, 855808, 921088, 986368, 1051648, 789509, 789764, 855044, 790019, 855299, 920579, 790274,
-    855554, 920834, 986114, 790529, 855809, 921089, 986369, 1051649, 790784, 856064, 921344, 986624,
-    1051904, 1117184, 1181187, 1181442, 1246722, 1181697, 1312257, 1246977, 1181952, 1247232, 1312512, 1377792,
-    1181188, 1181443, 1246723, 1181698, 1246978, 1312258, 1181953, 1247233, 1312513, 1377793, 1182208, 1247488,
-    1312768, 1378048, 1443328, 1181189, 1181444, 1246724, 1181699, 1246979, 1312259, 1181954, 1247234, 1312514,
-    1377794, 1182209, 1247489, 1312769, 1378049, 1443329, 1182464, 1247744, 1313024, 1378304, 1443584, 1508864,
-    1572867, 1573122, 1638402, 1573377, 1703937, 1638657, 1573632, 1638912, 1704192, 1769472, 1572868, 1573123,
-    1638403, 1573378, 1638658, 1703938, 1573633, 1638913, 1704193, 1769473, 1573888, 1639168, 1704448, 1769728,
-    1835008, 1572869, 1573124, 1638404, 1573379, 1638659, 1703939, 1573634, 1638914, 1704194, 1769474, 1573889,
-    1639169, 1704449, 1769729, 1835009, 1574144, 1639424, 1704704, 1769984, 1835264, 1900544, 33, 288,
-    65568, 543, 131103, 65823, 798, 66078, 131358, 196638, 34, 289, 65569, 544,
-    65824, 131104, 799, 66079, 131359, 196639, 1054, 66334, 131614, 196894, 262174, 35,
-    290, 65570, 545, 65825, 131105, 800, 66080, 131360, 196640, 1055, 66335, 131615,
-    196895, 262175, 1310, 66590, 131870, 197150, 262430, 327710, 1563, 1818, 67098, 2073,
-    132633, 67353, 2328, 67608, 132888, 198168, 1564, 1819, 67099, 2074, 67354, 132634,
-    2329, 67609, 132889, 198169, 2584, 67864, 133144, 198424, 263704, 1565, 1820, 67100,
-    2075, 67355, 132635, 2330, 67610, 132890, 198170, 2585, 67865, 133145, 198425, 263705,
-    2840, 68120, 133400, 198680, 263960, 329240, 393243, 393498, 458778, 393753, 524313, 459033,
-    394008, 459288, 524568, 589848, 393244, 393499, 458779, 393754, 459034, 524314, 394009, 459289,
-    524569, 589849, 394264, 459544, 524824, 590104, 655384, 393245, 393500, 458780, 393755, 459035,
-    524315, 394010, 459290, 524570, 589850, 394265, 459545, 524825, 590105, 655385, 394520, 459800,
-    525080, 590360, 655640, 720920, 3093, 3348, 68628, 3603, 134163, 68883, 3858, 69138,
-    134418, 199698, 3094, 3349, 68629, 3604, 68884, 134164, 3859, 69139, 134419, 199699,
-    4114, 69394, 134674, 199954, 265234, 3095, 3350, 68630, 3605, 68885, 134165, 3860,
-    69140, 134420, 199700, 4115, 69395, 134675, 199955, 265235, 4370, 69650, 134930, 200210,
-    265490, 330770, 394773, 395028, 460308, 395283, 525843, 460563, 395538, 460818, 526098, 591378,
-    394774, 395029, 460309, 395284, 460564, 525844, 395539, 460819, 526099, 591379, 395794, 461074,
-    526354, 591634, 656914, 394775, 395030, 460310, 395285, 460565, 525845, 395540, 460820, 526100,
-    591380, 395795, 461075, 526355, 591635, 656915, 396050, 461330, 526610, 591890, 657170, 722450,
-    786453, 786708, 851988, 786963, 917523, 852243, 787218, 852498, 917778, 983058, 786454, 786709,
-    851989, 786964, 852244, 917524, 787219, 852499, 917779, 983059, 787474, 852754, 918034, 983314,
-    1048594, 786455, 786710, 851990, 786965, 852245, 917525, 787220, 852500, 917780, 983060, 787475,
-    852755, 918035, 983315, 1048595, 787730, 853010, 918290, 983570, 1048850, 1114130, 4623, 4878,
-    70158, 5133, 135693, 70413, 5388, 70668, 135948, 201228, 4624, 4879, 70159, 5134,
-    70414, 135694, 5389, 70669, 135949, 201229, 5644, 70924, 136204, 201484, 266764, 4625,
-    4880, 70160, 5135, 70415, 135695, 5390, 70670, 135950, 201230, 5645, 70925, 136205,
-    201485, 266765, 5900, 71180, 136460, 201740, 267020, 332300, 396303, 396558, 461838, 396813,
-    527373, 462093, 397068, 462348, 527628, 592908, 396304, 396559, 461839, 396814, 462094, 527374,
-    397069, 462349, 527629, 592909, 397324, 462604, 527884, 593164, 658444, 396305, 396560, 461840,
-    396815, 462095, 527375, 397070, 462350, 527630, 592910, 397325, 462605, 527885, 593165, 658445,
-    397580, 462860, 528140, 593420, 658700, 723980, 787983, 788238, 853518, 788493, 919053, 853773,
-    788748, 854028, 919308, 984588, 787984, 788239, 853519, 788494, 853774, 919054, 788749, 854029,
-    919309, 984589, 789004, 854284, 919564, 984844, 1050124, 787985, 788240, 853520, 788495, 853775,
-    919055, 788750, 854030, 919310, 984590, 789005, 854285, 919565, 984845, 1050125, 789260, 854540,
-    919820, 985100, 1050380, 1115660, 1179663, 1179918, 1245198, 1180173, 1310733, 1245453, 1180428, 1245708,
-    1310988, 1376268, 1179664, 1179919, 1245199, 1180174, 1245454, 1310734, 1180429, 1245709, 1310989, 1376269,
-    1180684, 1245964, 1311244, 1376524, 1441804, 1179665, 1179920, 1245200, 1180175, 1245455, 1310735, 1180430,
-    1245710, 1310990, 1376270, 1180685, 1245965, 1311245, 1376525, 1441805, 1180940, 1246220, 1311500, 1376780,
-    1442060, 1507340, 6153, 6408, 71688, 6663, 137223, 71943, 6918, 72198, 137478, 202758,
-    6154, 6409, 71689, 6664, 71944, 137224, 6919, 72199, 137479, 202759, 7174, 72454,
-    137734, 203014, 268294, 6155, 6410, 71690, 6665, 71945, 137225, 6920, 72200, 137480,
-    202760, 7175, 72455, 137735, 203015, 268295, 7430, 72710, 137990, 203270, 268550, 333830,
-    397833, 398088, 463368, 398343, 528903, 463623, 398598, 463878, 529158, 594438, 397834, 398089,
-    463369, 398344, 463624, 528904, 398599, 463879, 529159, 594439, 398854, 464134, 529414, 594694,
-    659974, 397835, 398090, 463370, 398345, 463625, 528905, 398600, 463880, 529160, 594440, 398855,
-    464135, 529415, 594695, 659975, 399110, 464390, 529670, 594950, 660230, 725510, 789513, 789768,
-    855048, 790023, 920583, 855303, 790278, 855558, 920838, 986118, 789514, 789769, 855049, 790024,
-    855304, 920584, 790279, 855559, 920839, 986119, 790534, 855814, 921094, 986374, 1051654, 789515,
-    789770, 855050, 790025, 855305, 920585, 790280, 855560, 920840, 986120, 790535, 855815, 921095,
-    986375, 1051655, 790790, 856070, 921350, 986630, 1051910, 1117190, 1181193, 1181448, 1246728, 1181703,
-    1312263, 1246983, 1181958, 1247238, 1312518, 1377798, 1181194, 1181449, 1246729, 1181704, 1246984, 1312264,
-    1181959, 1247239, 1312519, 1377799, 1182214, 1247494, 1312774, 1378054, 1443334, 1181195, 1181450, 1246730,
-    1181705, 1246985, 1312265, 1181960, 1247240, 1312520, 1377800, 1182215, 1247495, 1312775, 1378055, 1443335,
-    1182470, 1247750, 1313030, 1378310, 1443590, 1508870, 1572873, 1573128, 1638408, 1573383, 1703943, 1638663,
-    1573638, 1638918, 1704198, 1769478, 1572874, 1573129, 1638409, 1573384, 1638664, 1703944, 1573639, 1638919,
-    1704199, 1769479, 1573894, 1639174, 1704454, 1769734, 1835014, 1572875, 1573130, 1638410, 1573385, 1638665,
-    1703945, 1573640, 1638920, 1704200, 1769480, 1573895, 1639175, 1704455, 1769735, 1835015, 1574150, 1639430,
-    1704710, 1769990, 1835270, 1900550, 7683, 7938, 73218, 8193, 138753, 73473, 8448, 73728,
-    139008, 204288, 7684, 7939, 73219, 8194, 73474, 138754, 8449, 73729, 139009, 204289,
-    8704, 73984, 139264, 204544, 269824, 7685, 7940, 73220, 8195, 73475, 138755, 8450,
-    73730, 139010, 204290, 8705, 73985, 139265, 204545, 269825, 8960, 74240, 139520, 204800,
-    270080, 335360, 399363, 399618, 464898, 399873, 530433, 465153, 400128, 465408, 530688, 595968,
-    399364, 399619, 464899, 399874, 465154, 530434, 400129, 465409, 530689, 595969, 400384, 465664,
-    530944, 596224, 661504, 399365, 399620, 464900, 399875, 465155, 530435, 400130, 465410, 530690,
-    595970, 400385, 465665, 530945, 596225, 661505, 400640, 465920, 531200, 596480, 661760, 727040,
-    791043, 791298, 856578, 791553, 922113, 856833, 791808, 857088, 922368, 987648, 791044, 791299,
-    856579, 791554, 856834, 922114, 791809, 857089, 922369, 987649, 792064, 857344, 922624, 987904,
-    1053184, 791045, 791300, 856580, 791555, 856835, 922115, 791810, 857090, 922370, 987650, 792065,
-    857345, 922625, 987905, 1053185, 792320, 857600, 922880, 988160, 1053440, 1118720, 1182723, 1182978,
-    1248258, 1183233, 1313793, 1248513, 1183488, 1248768, 1314048, 1379328, 1182724, 1182979, 1248259, 1183234,
-    1248514, 1313794, 1183489, 1248769, 1314049, 1379329, 1183744, 1249024, 1314304, 1379584, 1444864, 1182725,
-    1182980, 1248260, 1183235, 1248515, 1313795, 1183490, 1248770, 1314050, 1379330, 1183745, 1249025, 1314305,
-    1379585, 1444865, 1184000, 1249280, 1314560, 1379840, 1445120, 1510400, 1574403, 1574658, 1639938, 1574913,
-    1705473, 1640193, 1575168, 1640448, 1705728, 1771008, 1574404, 1574659, 1639939, 1574914, 1640194, 1705474,
-    1575169, 1640449, 1705729, 1771009, 1575424, 1640704, 1705984, 1771264, 1836544, 1574405, 1574660, 1639940,
-    1574915, 1640195, 1705475, 1575170, 1640450, 1705730, 1771010, 1575425, 1640705, 1705985, 1771265, 1836545,
-    1575680, 1640960, 1706240, 1771520, 1836800, 1902080, 1966083, 1966338, 2031618, 1966593, 2097153, 2031873,
-    1966848, 2032128, 2097408, 2162688, 1966084, 1966339, 2031619, 1966594, 2031874, 2097154, 1966849, 2032129,
-    2097409, 2162689, 1967104, 2032384, 2097664, 2162944, 2228224, 1966085, 1966340, 2031620, 1966595, 2031875,
-    2097155, 1966850, 2032130, 2097410, 2162690, 1967105, 2032385, 2097665, 2162945, 2228225, 1967360, 2032640,
-    2097920, 2163200, 2228480, 2293760,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_fdfd[61] = {
-    0, 3, 7, 11, 14, 18, 21, 24, 28, 32, 35, 39,
-    42, 45, 49, 53, 56, 60, 63, 66, 70, 74, 77, 81,
-    84, 87, 91, 95, 98, 102, 105, 108, 112, 116, 119, 123,
-    126, 129, 133, 137, 140, 144, 147, 150, 154, 158, 161, 165,
-    168, 171, 175, 179, 182, 186, 189, 192, 196, 200, 203, 207,
-    210,
-};
-__device__ const uint32_t kBraTerm_fdfd[210] = {
-    66560, 131338, 65561, 66816, 65803, 66058, 65562, 67072, 65804, 66314, 65563, 67328,
-    131595, 65564, 67584, 66060, 66315, 65565, 67840, 131852, 65566, 66561, 131339, 65562,
-    66817, 65805, 66059, 65564, 67073, 65806, 66315, 65565, 67329, 131597, 65567, 67585,
-    66062, 66317, 65568, 67841, 131854, 65569, 66562, 131340, 65563, 66818, 65806, 66060,
-    65565, 67074, 65807, 66316, 65566, 67330, 131598, 65568, 67586, 66063, 66318, 65569,
-    67842, 131855, 65570, 66563, 131341, 65564, 66819, 65808, 66061, 65567, 67075, 65809,
-    66317, 65568, 67331, 131600, 65571, 67587, 66065, 66320, 65572, 67843, 131857, 65573,
-    66564, 131343, 65566, 66820, 65810, 66063, 65569, 67076, 65811, 66319, 65570, 67332,
-    131602, 65573, 67588, 66067, 66322, 65574, 67844, 131859, 65575, 66565, 131342, 65565,
-    66821, 65809, 66062, 65568, 67077, 65810, 66318, 65569, 67333, 131601, 65572, 67589,
-    66066, 66321, 65573, 67845, 131858, 65574, 66566, 131344, 65567, 66822, 65812, 66064,
-    65571, 67078, 65813, 66320, 65572, 67334, 131604, 65576, 67590, 66069, 66324, 65577,
-    67846, 131861, 65578, 66567, 131345, 65568, 66823, 65813, 66065, 65572, 67079, 65814,
-    66321, 65573, 67335, 131605, 65577, 67591, 66070, 66325, 65578, 67847, 131862, 65579,
-    66568, 131346, 65569, 66824, 65814, 66066, 65573, 67080, 65815, 66322, 65574, 67336,
-    131606, 65578, 67592, 66071, 66326, 65579, 67848, 131863, 65580, 66569, 131347, 65570,
-    66825, 65815, 66067, 65574, 67081, 65816, 66323, 65575, 67337, 131607, 65579, 67593,
-    66072, 66327, 65580, 67849, 131864, 65581,
-};
-__device__ const uint16_t kKetOff_fdfd[61] = {
-    0, 3, 7, 11, 14, 18, 21, 24, 28, 32, 35, 39,
-    42, 45, 49, 53, 56, 60, 63, 66, 70, 74, 77, 81,
-    84, 87, 91, 95, 98, 102, 105, 108, 112, 116, 119, 123,
-    126, 129, 133, 137, 140, 144, 147, 150, 154, 158, 161, 165,
-    168, 171, 175, 179, 182, 186, 189, 192, 196, 200, 203, 207,
-    210,
-};
-__device__ const uint32_t kKetTerm_fdfd[210] = {
-    66560, 131338, 65561, 66816, 65803, 66058, 65562, 67072, 65804, 66314, 65563, 67328,
-    131595, 65564, 67584, 66060, 66315, 65565, 67840, 131852, 65566, 66561, 131339, 65562,
-    66817, 65805, 66059, 65564, 67073, 65806, 66315, 65565, 67329, 131597, 65567, 67585,
-    66062, 66317, 65568, 67841, 131854, 65569, 66562, 131340, 65563, 66818, 65806, 66060,
-    65565, 67074, 65807, 66316, 65566, 67330, 131598, 65568, 67586, 66063, 66318, 65569,
-    67842, 131855, 65570, 66563, 131341, 65564, 66819, 65808, 66061, 65567, 67075, 65809,
-    66317, 65568, 67331, 131600, 65571, 67587, 66065, 66320, 65572, 67843, 131857, 65573,
-    66564, 131343, 65566, 66820, 65810, 66063, 65569, 67076, 65811, 66319, 65570, 67332,
-    131602, 65573, 67588, 66067, 66322, 65574, 67844, 131859, 65575, 66565, 131342, 65565,
-    66821, 65809, 66062, 65568, 67077, 65810, 66318, 65569, 67333, 131601, 65572, 67589,
-    66066, 66321, 65573, 67845, 131858, 65574, 66566, 131344, 65567, 66822, 65812, 66064,
-    65571, 67078, 65813, 66320, 65572, 67334, 131604, 65576, 67590, 66069, 66324, 65577,
-    67846, 131861, 65578, 66567, 131345, 65568, 66823, 65813, 66065, 65572, 67079, 65814,
-    66321, 65573, 67335, 131605, 65577, 67591, 66070, 66325, 65578, 67847, 131862, 65579,
-    66568, 131346, 65569, 66824, 65814, 66066, 65573, 67080, 65815, 66322, 65574, 67336,
-    131606, 65578, 67592, 66071, 66326, 65579, 67848, 131863, 65580, 66569, 131347, 65570,
-    66825, 65815, 66067, 65574, 67081, 65816, 66323, 65575, 67337, 131607, 65579, 67593,
-    66072, 66327, 65580, 67849, 131864, 65581,
-};
 __device__ const double kNormAB_fdfd[60] = {
     0.14907119849998599, 0.2581988897471611, 0.2581988897471611, 0.14907119849998599,
     0.2581988897471611, 0.14907119849998599, 0.3333333333333334, 0.5773502691896258,
@@ -322,31 +468,12 @@ __device__ const double kNormAB_fdfd[60] = {
     0.5773502691896258, 0.3333333333333334, 0.14907119849998599, 0.2581988897471611,
     0.2581988897471611, 0.14907119849998599, 0.2581988897471611, 0.14907119849998599,
 };
-__device__ const double kNormCD_fdfd[60] = {
-    0.14907119849998599, 0.2581988897471611, 0.2581988897471611, 0.14907119849998599,
-    0.2581988897471611, 0.14907119849998599, 0.3333333333333334, 0.5773502691896258,
-    0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 0.3333333333333334,
-    0.3333333333333334, 0.5773502691896258, 0.5773502691896258, 0.3333333333333334,
-    0.5773502691896258, 0.3333333333333334, 0.3333333333333334, 0.5773502691896258,
-    0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 0.3333333333333334,
-    0.3333333333333334, 0.5773502691896258, 0.5773502691896258, 0.3333333333333334,
-    0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 1.0,
-    1.0, 0.5773502691896258, 1.0, 0.5773502691896258,
-    0.14907119849998599, 0.2581988897471611, 0.2581988897471611, 0.14907119849998599,
-    0.2581988897471611, 0.14907119849998599, 0.3333333333333334, 0.5773502691896258,
-    0.5773502691896258, 0.3333333333333334, 0.5773502691896258, 0.3333333333333334,
-    0.3333333333333334, 0.5773502691896258, 0.5773502691896258, 0.3333333333333334,
-    0.5773502691896258, 0.3333333333333334, 0.14907119849998599, 0.2581988897471611,
-    0.2581988897471611, 0.14907119849998599, 0.2581988897471611, 0.14907119849998599,
-};
-
 
 // column components cx | cy << 4 | cz << 8
 __device__ const uint16_t kCol_fdfd[46] = { 3, 18, 258, 33, 513, 273, 48, 288, 528, 768, 4, 19, 259, 34, 274, 514, 49, 289, 529, 769, 64, 304, 544, 784, 1024, 5, 20, 260, 35, 275, 515, 50, 290, 530, 770, 65, 305, 545, 785, 1025, 80, 320, 560, 800, 1040, 1280 };
 
 __device__ __forceinline__ RysClassTabs tabs_fdfd() {
-    return RysClassTabs{kBlk_fdfd, kBraOff_fdfd, kBraTerm_fdfd, kKetOff_fdfd, kKetTerm_fdfd,
-                        kNormAB_fdfd, kNormCD_fdfd, kCol_fdfd};
+    return RysClassTabs{kNormAB_fdfd, kCol_fdfd};
 }
 
 template <int MIXED>
@@ -364,9 +491,9 @@ static void rys_prepare_fdfd() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_fdfd<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 93952);
-        cudaFuncSetAttribute(rys_queue_fdfd<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 93952);
-        cudaFuncSetAttribute(rys_bound_kernel_fdfd, cudaFuncAttributeMaxDynamicSharedMemorySize, 93952);
+        cudaFuncSetAttribute(rys_queue_fdfd<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 103680);
+        cudaFuncSetAttribute(rys_queue_fdfd<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 103680);
+        cudaFuncSetAttribute(rys_bound_kernel_fdfd, cudaFuncAttributeMaxDynamicSharedMemorySize, 103680);
         done[dev] = true;
     }
 }
@@ -377,16 +504,16 @@ void launch_rys_fdfd(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_fdfd();
     constexpr int ng = 128 / C_fdfd::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_fdfd<1><<<grid, 128, 93952, s>>>(Q, R);
-    else rys_queue_fdfd<0><<<grid, 128, 93952, s>>>(Q, R);
+    if (mixed) rys_queue_fdfd<1><<<grid, 128, 103680, s>>>(Q, R);
+    else rys_queue_fdfd<0><<<grid, 128, 103680, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_fdfd(int mixed) {
     rys_prepare_fdfd();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fdfd<1>, 128, 93952);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fdfd<0>, 128, 93952);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fdfd<1>, 128, 103680);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fdfd<0>, 128, 103680);
     return n;
 }
 
@@ -395,7 +522,7 @@ void launch_rys_bound_fdfd(const PairTab &P, const RysTab &R, int p0, int np, do
     if (np <= 0) return;
     rys_prepare_fdfd();
     constexpr int ng = 128 / C_fdfd::G;
-    rys_bound_kernel_fdfd<<<(np + ng - 1) / ng, 128, 93952, s>>>(P, R, p0, np, pbound, qout, full);
+    rys_bound_kernel_fdfd<<<(np + ng - 1) / ng, 128, 103680, s>>>(P, R, p0, np, pbound, qout, full);
 }
 
 }  // namespace molints

@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (fd|fp).  Do not edit.
-// roots 5, block 46 x 25, outputs 60 x 30, group 32 threads,
-// 6 primitive quartets per batch, 1 slot(s), 1 accumulators per thread, 87680 B shared per block, column mode.
+// roots 5, block 46 x 25, outputs 60 x 30, group 32 threads, 1 ket pairs a round,
+// 6 primitive quartets per ket pair and batch, 107520 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,11 +11,10 @@ struct C_fdfp {
     static constexpr int NA = 46, NC = 25, NBLK = 1150;
     static constexpr int NB = 6, ND = 3;
     static constexpr int NAB = 60, NCD = 30;
-    static constexpr int G = 32, NPB = 6, NSLOT = 1, ACC = 1;
-    static constexpr int S = 30;
-    static constexpr int SMEM_GROUP = 2740;
-    static constexpr bool COL = true;
-    // stage 2, column mode: acc[row] += x[ax] y[ay] z[az] for the column's table columns
+    static constexpr int G = 32, W = 1, H = 1, PB = 6;
+    static constexpr int S = 30, SI = 91, NCP = 25, NCDP = 31;
+    static constexpr int SMEM_GROUP = 3360;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
     __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
         acc[0] = fma(x[3] * y[0], z[0], acc[0]);
@@ -65,149 +64,264 @@ struct C_fdfp {
         acc[44] = fma(x[0] * y[1], z[4], acc[44]);
         acc[45] = fma(x[0] * y[0], z[5], acc[45]);
     }
-    static constexpr int NCOLS = 25;
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[10], in[25]);
+        const double h1 = fma(x, in[0], in[10]);
+        const double h2 = fma(x, h1, h0);
+        const double h3 = fma(y, in[10], in[26]);
+        const double h4 = fma(y, in[0], in[11]);
+        const double h5 = fma(x, h4, h3);
+        const double h6 = fma(z, in[10], in[27]);
+        const double h7 = fma(z, in[0], in[12]);
+        const double h8 = fma(x, h7, h6);
+        const double h9 = fma(y, in[11], in[28]);
+        const double h10 = fma(y, h4, h9);
+        const double h11 = fma(z, in[11], in[29]);
+        const double h12 = fma(y, h7, h11);
+        const double h13 = fma(z, in[12], in[30]);
+        const double h14 = fma(z, h7, h13);
+        const double h15 = fma(x, in[11], in[26]);
+        const double h16 = fma(x, in[1], in[11]);
+        const double h17 = fma(x, h16, h15);
+        const double h18 = fma(y, in[1], in[13]);
+        const double h19 = fma(x, h18, h9);
+        const double h20 = fma(z, in[1], in[14]);
+        const double h21 = fma(x, h20, h11);
+        const double h22 = fma(y, in[13], in[31]);
+        const double h23 = fma(y, h18, h22);
+        const double h24 = fma(z, in[13], in[32]);
+        const double h25 = fma(y, h20, h24);
+        const double h26 = fma(z, in[14], in[33]);
+        const double h27 = fma(z, h20, h26);
+        const double h28 = fma(x, in[12], in[27]);
+        const double h29 = fma(x, in[2], in[12]);
+        const double h30 = fma(x, h29, h28);
+        const double h31 = fma(y, in[12], in[29]);
+        const double h32 = fma(y, in[2], in[14]);
+        const double h33 = fma(x, h32, h31);
+        const double h34 = fma(z, in[2], in[15]);
+        const double h35 = fma(x, h34, h13);
+        const double h36 = fma(y, in[14], in[32]);
+        const double h37 = fma(y, h32, h36);
+        const double h38 = fma(y, h34, h26);
+        const double h39 = fma(z, in[15], in[34]);
+        const double h40 = fma(z, h34, h39);
+        const double h41 = fma(x, in[13], in[28]);
+        const double h42 = fma(x, in[3], in[13]);
+        const double h43 = fma(x, h42, h41);
+        const double h44 = fma(y, in[3], in[16]);
+        const double h45 = fma(x, h44, h22);
+        const double h46 = fma(z, in[3], in[17]);
+        const double h47 = fma(x, h46, h24);
+        const double h48 = fma(y, in[16], in[35]);
+        const double h49 = fma(y, h44, h48);
+        const double h50 = fma(z, in[16], in[36]);
+        const double h51 = fma(y, h46, h50);
+        const double h52 = fma(z, in[17], in[37]);
+        const double h53 = fma(z, h46, h52);
+        const double h54 = fma(x, in[15], in[30]);
+        const double h55 = fma(x, in[4], in[15]);
+        const double h56 = fma(x, h55, h54);
+        const double h57 = fma(y, in[15], in[33]);
+        const double h58 = fma(y, in[4], in[18]);
+        const double h59 = fma(x, h58, h57);
+        const double h60 = fma(z, in[4], in[19]);
+        const double h61 = fma(x, h60, h39);
+        const double h62 = fma(y, in[18], in[37]);
+        const double h63 = fma(y, h58, h62);
+        const double h64 = fma(z, in[18], in[38]);
+        const double h65 = fma(y, h60, h64);
+        const double h66 = fma(z, in[19], in[39]);
+        const double h67 = fma(z, h60, h66);
+        const double h68 = fma(x, in[14], in[29]);
+        const double h69 = fma(x, in[5], in[14]);
+        const double h70 = fma(x, h69, h68);
+        const double h71 = fma(y, in[5], in[17]);
+        const double h72 = fma(x, h71, h36);
+        const double h73 = fma(z, in[5], in[18]);
+        const double h74 = fma(x, h73, h26);
+        const double h75 = fma(y, in[17], in[36]);
+        const double h76 = fma(y, h71, h75);
+        const double h77 = fma(y, h73, h52);
+        const double h78 = fma(z, h73, h64);
+        const double h79 = fma(x, in[16], in[31]);
+        const double h80 = fma(x, in[6], in[16]);
+        const double h81 = fma(x, h80, h79);
+        const double h82 = fma(y, in[6], in[20]);
+        const double h83 = fma(x, h82, h48);
+        const double h84 = fma(z, in[6], in[21]);
+        const double h85 = fma(x, h84, h50);
+        const double h86 = fma(y, in[20], in[40]);
+        const double h87 = fma(y, h82, h86);
+        const double h88 = fma(z, in[20], in[41]);
+        const double h89 = fma(y, h84, h88);
+        const double h90 = fma(z, in[21], in[42]);
+        const double h91 = fma(z, h84, h90);
+        const double h92 = fma(x, in[17], in[32]);
+        const double h93 = fma(x, in[7], in[17]);
+        const double h94 = fma(x, h93, h92);
+        const double h95 = fma(y, in[7], in[21]);
+        const double h96 = fma(x, h95, h75);
+        const double h97 = fma(z, in[7], in[22]);
+        const double h98 = fma(x, h97, h52);
+        const double h99 = fma(y, in[21], in[41]);
+        const double h100 = fma(y, h95, h99);
+        const double h101 = fma(y, h97, h90);
+        const double h102 = fma(z, in[22], in[43]);
+        const double h103 = fma(z, h97, h102);
+        const double h104 = fma(x, in[18], in[33]);
+        const double h105 = fma(x, in[8], in[18]);
+        const double h106 = fma(x, h105, h104);
+        const double h107 = fma(y, in[8], in[22]);
+        const double h108 = fma(x, h107, h62);
+        const double h109 = fma(z, in[8], in[23]);
+        const double h110 = fma(x, h109, h64);
+        const double h111 = fma(y, in[22], in[42]);
+        const double h112 = fma(y, h107, h111);
+        const double h113 = fma(y, h109, h102);
+        const double h114 = fma(z, in[23], in[44]);
+        const double h115 = fma(z, h109, h114);
+        const double h116 = fma(x, in[19], in[34]);
+        const double h117 = fma(x, in[9], in[19]);
+        const double h118 = fma(x, h117, h116);
+        const double h119 = fma(y, in[19], in[38]);
+        const double h120 = fma(y, in[9], in[23]);
+        const double h121 = fma(x, h120, h119);
+        const double h122 = fma(z, in[9], in[24]);
+        const double h123 = fma(x, h122, h66);
+        const double h124 = fma(y, in[23], in[43]);
+        const double h125 = fma(y, h120, h124);
+        const double h126 = fma(y, h122, h114);
+        const double h127 = fma(z, in[24], in[45]);
+        const double h128 = fma(z, h122, h127);
+        out[0] = h2;
+        out[25] = h5;
+        out[50] = h8;
+        out[75] = h10;
+        out[100] = h12;
+        out[125] = h14;
+        out[150] = h17;
+        out[175] = h19;
+        out[200] = h21;
+        out[225] = h23;
+        out[250] = h25;
+        out[275] = h27;
+        out[300] = h30;
+        out[325] = h33;
+        out[350] = h35;
+        out[375] = h37;
+        out[400] = h38;
+        out[425] = h40;
+        out[450] = h43;
+        out[475] = h45;
+        out[500] = h47;
+        out[525] = h49;
+        out[550] = h51;
+        out[575] = h53;
+        out[600] = h56;
+        out[625] = h59;
+        out[650] = h61;
+        out[675] = h63;
+        out[700] = h65;
+        out[725] = h67;
+        out[750] = h70;
+        out[775] = h72;
+        out[800] = h74;
+        out[825] = h76;
+        out[850] = h77;
+        out[875] = h78;
+        out[900] = h81;
+        out[925] = h83;
+        out[950] = h85;
+        out[975] = h87;
+        out[1000] = h89;
+        out[1025] = h91;
+        out[1050] = h94;
+        out[1075] = h96;
+        out[1100] = h98;
+        out[1125] = h100;
+        out[1150] = h101;
+        out[1175] = h103;
+        out[1200] = h106;
+        out[1225] = h108;
+        out[1250] = h110;
+        out[1275] = h112;
+        out[1300] = h113;
+        out[1325] = h115;
+        out[1350] = h118;
+        out[1375] = h121;
+        out[1400] = h123;
+        out[1425] = h125;
+        out[1450] = h126;
+        out[1475] = h128;
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[0], in[10]);
+        const double h1 = fma(y, in[0], in[11]);
+        const double h2 = fma(z, in[0], in[12]);
+        const double h3 = fma(x, in[1], in[11]);
+        const double h4 = fma(y, in[1], in[13]);
+        const double h5 = fma(z, in[1], in[14]);
+        const double h6 = fma(x, in[2], in[12]);
+        const double h7 = fma(y, in[2], in[14]);
+        const double h8 = fma(z, in[2], in[15]);
+        const double h9 = fma(x, in[3], in[13]);
+        const double h10 = fma(y, in[3], in[16]);
+        const double h11 = fma(z, in[3], in[17]);
+        const double h12 = fma(x, in[4], in[15]);
+        const double h13 = fma(y, in[4], in[18]);
+        const double h14 = fma(z, in[4], in[19]);
+        const double h15 = fma(x, in[5], in[14]);
+        const double h16 = fma(y, in[5], in[17]);
+        const double h17 = fma(z, in[5], in[18]);
+        const double h18 = fma(x, in[6], in[16]);
+        const double h19 = fma(y, in[6], in[20]);
+        const double h20 = fma(z, in[6], in[21]);
+        const double h21 = fma(x, in[7], in[17]);
+        const double h22 = fma(y, in[7], in[21]);
+        const double h23 = fma(z, in[7], in[22]);
+        const double h24 = fma(x, in[8], in[18]);
+        const double h25 = fma(y, in[8], in[22]);
+        const double h26 = fma(z, in[8], in[23]);
+        const double h27 = fma(x, in[9], in[19]);
+        const double h28 = fma(y, in[9], in[23]);
+        const double h29 = fma(z, in[9], in[24]);
+        out[0] = h0 * (nrm * 0.2581988897471611);
+        out[1] = h1 * (nrm * 0.2581988897471611);
+        out[2] = h2 * (nrm * 0.2581988897471611);
+        out[3] = h3 * (nrm * 0.5773502691896258);
+        out[4] = h4 * (nrm * 0.5773502691896258);
+        out[5] = h5 * (nrm * 0.5773502691896258);
+        out[6] = h6 * (nrm * 0.5773502691896258);
+        out[7] = h7 * (nrm * 0.5773502691896258);
+        out[8] = h8 * (nrm * 0.5773502691896258);
+        out[9] = h9 * (nrm * 0.5773502691896258);
+        out[10] = h10 * (nrm * 0.5773502691896258);
+        out[11] = h11 * (nrm * 0.5773502691896258);
+        out[12] = h12 * (nrm * 0.5773502691896258);
+        out[13] = h13 * (nrm * 0.5773502691896258);
+        out[14] = h14 * (nrm * 0.5773502691896258);
+        out[15] = h15 * (nrm * 1.0);
+        out[16] = h16 * (nrm * 1.0);
+        out[17] = h17 * (nrm * 1.0);
+        out[18] = h18 * (nrm * 0.2581988897471611);
+        out[19] = h19 * (nrm * 0.2581988897471611);
+        out[20] = h20 * (nrm * 0.2581988897471611);
+        out[21] = h21 * (nrm * 0.5773502691896258);
+        out[22] = h22 * (nrm * 0.5773502691896258);
+        out[23] = h23 * (nrm * 0.5773502691896258);
+        out[24] = h24 * (nrm * 0.5773502691896258);
+        out[25] = h25 * (nrm * 0.5773502691896258);
+        out[26] = h26 * (nrm * 0.5773502691896258);
+        out[27] = h27 * (nrm * 0.2581988897471611);
+        out[28] = h28 * (nrm * 0.2581988897471611);
+        out[29] = h29 * (nrm * 0.2581988897471611);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_fdfp[1150] = {
-    18, 273, 65553, 528, 131088, 65808, 783, 66063, 131343, 196623, 19, 274,
-    65554, 529, 65809, 131089, 784, 66064, 131344, 196624, 1039, 66319, 131599, 196879,
-    262159, 1293, 1548, 66828, 1803, 132363, 67083, 2058, 67338, 132618, 197898, 1294,
-    1549, 66829, 1804, 67084, 132364, 2059, 67339, 132619, 197899, 2314, 67594, 132874,
-    198154, 263434, 327693, 327948, 393228, 328203, 458763, 393483, 328458, 393738, 459018, 524298,
-    327694, 327949, 393229, 328204, 393484, 458764, 328459, 393739, 459019, 524299, 328714, 393994,
-    459274, 524554, 589834, 2568, 2823, 68103, 3078, 133638, 68358, 3333, 68613, 133893,
-    199173, 2569, 2824, 68104, 3079, 68359, 133639, 3334, 68614, 133894, 199174, 3589,
-    68869, 134149, 199429, 264709, 655368, 655623, 720903, 655878, 786438, 721158, 656133, 721413,
-    786693, 851973, 655369, 655624, 720904, 655879, 721159, 786439, 656134, 721414, 786694, 851974,
-    656389, 721669, 786949, 852229, 917509, 328968, 329223, 394503, 329478, 460038, 394758, 329733,
-    395013, 460293, 525573, 328969, 329224, 394504, 329479, 394759, 460039, 329734, 395014, 460294,
-    525574, 329989, 395269, 460549, 525829, 591109, 3843, 4098, 69378, 4353, 134913, 69633,
-    4608, 69888, 135168, 200448, 3844, 4099, 69379, 4354, 69634, 134914, 4609, 69889,
-    135169, 200449, 4864, 70144, 135424, 200704, 265984, 330243, 330498, 395778, 330753, 461313,
-    396033, 331008, 396288, 461568, 526848, 330244, 330499, 395779, 330754, 396034, 461314, 331009,
-    396289, 461569, 526849, 331264, 396544, 461824, 527104, 592384, 656643, 656898, 722178, 657153,
-    787713, 722433, 657408, 722688, 787968, 853248, 656644, 656899, 722179, 657154, 722434, 787714,
-    657409, 722689, 787969, 853249, 657664, 722944, 788224, 853504, 918784, 983043, 983298, 1048578,
-    983553, 1114113, 1048833, 983808, 1049088, 1114368, 1179648, 983044, 983299, 1048579, 983554, 1048834,
-    1114114, 983809, 1049089, 1114369, 1179649, 984064, 1049344, 1114624, 1179904, 1245184, 23, 278,
-    65558, 533, 131093, 65813, 788, 66068, 131348, 196628, 24, 279, 65559, 534,
-    65814, 131094, 789, 66069, 131349, 196629, 1044, 66324, 131604, 196884, 262164, 1298,
-    1553, 66833, 1808, 132368, 67088, 2063, 67343, 132623, 197903, 1299, 1554, 66834,
-    1809, 67089, 132369, 2064, 67344, 132624, 197904, 2319, 67599, 132879, 198159, 263439,
-    327698, 327953, 393233, 328208, 458768, 393488, 328463, 393743, 459023, 524303, 327699, 327954,
-    393234, 328209, 393489, 458769, 328464, 393744, 459024, 524304, 328719, 393999, 459279, 524559,
-    589839, 2573, 2828, 68108, 3083, 133643, 68363, 3338, 68618, 133898, 199178, 2574,
-    2829, 68109, 3084, 68364, 133644, 3339, 68619, 133899, 199179, 3594, 68874, 134154,
-    199434, 264714, 328973, 329228, 394508, 329483, 460043, 394763, 329738, 395018, 460298, 525578,
-    328974, 329229, 394509, 329484, 394764, 460044, 329739, 395019, 460299, 525579, 329994, 395274,
-    460554, 525834, 591114, 655373, 655628, 720908, 655883, 786443, 721163, 656138, 721418, 786698,
-    851978, 655374, 655629, 720909, 655884, 721164, 786444, 656139, 721419, 786699, 851979, 656394,
-    721674, 786954, 852234, 917514, 3848, 4103, 69383, 4358, 134918, 69638, 4613, 69893,
-    135173, 200453, 3849, 4104, 69384, 4359, 69639, 134919, 4614, 69894, 135174, 200454,
-    4869, 70149, 135429, 200709, 265989, 330248, 330503, 395783, 330758, 461318, 396038, 331013,
-    396293, 461573, 526853, 330249, 330504, 395784, 330759, 396039, 461319, 331014, 396294, 461574,
-    526854, 331269, 396549, 461829, 527109, 592389, 656648, 656903, 722183, 657158, 787718, 722438,
-    657413, 722693, 787973, 853253, 656649, 656904, 722184, 657159, 722439, 787719, 657414, 722694,
-    787974, 853254, 657669, 722949, 788229, 853509, 918789, 983048, 983303, 1048583, 983558, 1114118,
-    1048838, 983813, 1049093, 1114373, 1179653, 983049, 983304, 1048584, 983559, 1048839, 1114119, 983814,
-    1049094, 1114374, 1179654, 984069, 1049349, 1114629, 1179909, 1245189, 5123, 5378, 70658, 5633,
-    136193, 70913, 5888, 71168, 136448, 201728, 5124, 5379, 70659, 5634, 70914, 136194,
-    5889, 71169, 136449, 201729, 6144, 71424, 136704, 201984, 267264, 331523, 331778, 397058,
-    332033, 462593, 397313, 332288, 397568, 462848, 528128, 331524, 331779, 397059, 332034, 397314,
-    462594, 332289, 397569, 462849, 528129, 332544, 397824, 463104, 528384, 593664, 657923, 658178,
-    723458, 658433, 788993, 723713, 658688, 723968, 789248, 854528, 657924, 658179, 723459, 658434,
-    723714, 788994, 658689, 723969, 789249, 854529, 658944, 724224, 789504, 854784, 920064, 984323,
-    984578, 1049858, 984833, 1115393, 1050113, 985088, 1050368, 1115648, 1180928, 984324, 984579, 1049859,
-    984834, 1050114, 1115394, 985089, 1050369, 1115649, 1180929, 985344, 1050624, 1115904, 1181184, 1246464,
-    1310723, 1310978, 1376258, 1311233, 1441793, 1376513, 1311488, 1376768, 1442048, 1507328, 1310724, 1310979,
-    1376259, 1311234, 1376514, 1441794, 1311489, 1376769, 1442049, 1507329, 1311744, 1377024, 1442304, 1507584,
-    1572864, 28, 283, 65563, 538, 131098, 65818, 793, 66073, 131353, 196633, 29,
-    284, 65564, 539, 65819, 131099, 794, 66074, 131354, 196634, 1049, 66329, 131609,
-    196889, 262169, 1303, 1558, 66838, 1813, 132373, 67093, 2068, 67348, 132628, 197908,
-    1304, 1559, 66839, 1814, 67094, 132374, 2069, 67349, 132629, 197909, 2324, 67604,
-    132884, 198164, 263444, 327703, 327958, 393238, 328213, 458773, 393493, 328468, 393748, 459028,
-    524308, 327704, 327959, 393239, 328214, 393494, 458774, 328469, 393749, 459029, 524309, 328724,
-    394004, 459284, 524564, 589844, 2578, 2833, 68113, 3088, 133648, 68368, 3343, 68623,
-    133903, 199183, 2579, 2834, 68114, 3089, 68369, 133649, 3344, 68624, 133904, 199184,
-    3599, 68879, 134159, 199439, 264719, 328978, 329233, 394513, 329488, 460048, 394768, 329743,
-    395023, 460303, 525583, 328979, 329234, 394514, 329489, 394769, 460049, 329744, 395024, 460304,
-    525584, 329999, 395279, 460559, 525839, 591119, 655378, 655633, 720913, 655888, 786448, 721168,
-    656143, 721423, 786703, 851983, 655379, 655634, 720914, 655889, 721169, 786449, 656144, 721424,
-    786704, 851984, 656399, 721679, 786959, 852239, 917519, 3853, 4108, 69388, 4363, 134923,
-    69643, 4618, 69898, 135178, 200458, 3854, 4109, 69389, 4364, 69644, 134924, 4619,
-    69899, 135179, 200459, 4874, 70154, 135434, 200714, 265994, 330253, 330508, 395788, 330763,
-    461323, 396043, 331018, 396298, 461578, 526858, 330254, 330509, 395789, 330764, 396044, 461324,
-    331019, 396299, 461579, 526859, 331274, 396554, 461834, 527114, 592394, 656653, 656908, 722188,
-    657163, 787723, 722443, 657418, 722698, 787978, 853258, 656654, 656909, 722189, 657164, 722444,
-    787724, 657419, 722699, 787979, 853259, 657674, 722954, 788234, 853514, 918794, 983053, 983308,
-    1048588, 983563, 1114123, 1048843, 983818, 1049098, 1114378, 1179658, 983054, 983309, 1048589, 983564,
-    1048844, 1114124, 983819, 1049099, 1114379, 1179659, 984074, 1049354, 1114634, 1179914, 1245194, 5128,
-    5383, 70663, 5638, 136198, 70918, 5893, 71173, 136453, 201733, 5129, 5384, 70664,
-    5639, 70919, 136199, 5894, 71174, 136454, 201734, 6149, 71429, 136709, 201989, 267269,
-    331528, 331783, 397063, 332038, 462598, 397318, 332293, 397573, 462853, 528133, 331529, 331784,
-    397064, 332039, 397319, 462599, 332294, 397574, 462854, 528134, 332549, 397829, 463109, 528389,
-    593669, 657928, 658183, 723463, 658438, 788998, 723718, 658693, 723973, 789253, 854533, 657929,
-    658184, 723464, 658439, 723719, 788999, 658694, 723974, 789254, 854534, 658949, 724229, 789509,
-    854789, 920069, 984328, 984583, 1049863, 984838, 1115398, 1050118, 985093, 1050373, 1115653, 1180933,
-    984329, 984584, 1049864, 984839, 1050119, 1115399, 985094, 1050374, 1115654, 1180934, 985349, 1050629,
-    1115909, 1181189, 1246469, 1310728, 1310983, 1376263, 1311238, 1441798, 1376518, 1311493, 1376773, 1442053,
-    1507333, 1310729, 1310984, 1376264, 1311239, 1376519, 1441799, 1311494, 1376774, 1442054, 1507334, 1311749,
-    1377029, 1442309, 1507589, 1572869, 6403, 6658, 71938, 6913, 137473, 72193, 7168, 72448,
-    137728, 203008, 6404, 6659, 71939, 6914, 72194, 137474, 7169, 72449, 137729, 203009,
-    7424, 72704, 137984, 203264, 268544, 332803, 333058, 398338, 333313, 463873, 398593, 333568,
-    398848, 464128, 529408, 332804, 333059, 398339, 333314, 398594, 463874, 333569, 398849, 464129,
-    529409, 333824, 399104, 464384, 529664, 594944, 659203, 659458, 724738, 659713, 790273, 724993,
-    659968, 725248, 790528, 855808, 659204, 659459, 724739, 659714, 724994, 790274, 659969, 725249,
-    790529, 855809, 660224, 725504, 790784, 856064, 921344, 985603, 985858, 1051138, 986113, 1116673,
-    1051393, 986368, 1051648, 1116928, 1182208, 985604, 985859, 1051139, 986114, 1051394, 1116674, 986369,
-    1051649, 1116929, 1182209, 986624, 1051904, 1117184, 1182464, 1247744, 1312003, 1312258, 1377538, 1312513,
-    1443073, 1377793, 1312768, 1378048, 1443328, 1508608, 1312004, 1312259, 1377539, 1312514, 1377794, 1443074,
-    1312769, 1378049, 1443329, 1508609, 1313024, 1378304, 1443584, 1508864, 1574144, 1638403, 1638658, 1703938,
-    1638913, 1769473, 1704193, 1639168, 1704448, 1769728, 1835008, 1638404, 1638659, 1703939, 1638914, 1704194,
-    1769474, 1639169, 1704449, 1769729, 1835009, 1639424, 1704704, 1769984, 1835264, 1900544,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_fdfp[61] = {
-    0, 3, 7, 11, 14, 18, 21, 24, 28, 32, 35, 39,
-    42, 45, 49, 53, 56, 60, 63, 66, 70, 74, 77, 81,
-    84, 87, 91, 95, 98, 102, 105, 108, 112, 116, 119, 123,
-    126, 129, 133, 137, 140, 144, 147, 150, 154, 158, 161, 165,
-    168, 171, 175, 179, 182, 186, 189, 192, 196, 200, 203, 207,
-    210,
-};
-__device__ const uint32_t kBraTerm_fdfp[210] = {
-    66560, 131338, 65561, 66816, 65803, 66058, 65562, 67072, 65804, 66314, 65563, 67328,
-    131595, 65564, 67584, 66060, 66315, 65565, 67840, 131852, 65566, 66561, 131339, 65562,
-    66817, 65805, 66059, 65564, 67073, 65806, 66315, 65565, 67329, 131597, 65567, 67585,
-    66062, 66317, 65568, 67841, 131854, 65569, 66562, 131340, 65563, 66818, 65806, 66060,
-    65565, 67074, 65807, 66316, 65566, 67330, 131598, 65568, 67586, 66063, 66318, 65569,
-    67842, 131855, 65570, 66563, 131341, 65564, 66819, 65808, 66061, 65567, 67075, 65809,
-    66317, 65568, 67331, 131600, 65571, 67587, 66065, 66320, 65572, 67843, 131857, 65573,
-    66564, 131343, 65566, 66820, 65810, 66063, 65569, 67076, 65811, 66319, 65570, 67332,
-    131602, 65573, 67588, 66067, 66322, 65574, 67844, 131859, 65575, 66565, 131342, 65565,
-    66821, 65809, 66062, 65568, 67077, 65810, 66318, 65569, 67333, 131601, 65572, 67589,
-    66066, 66321, 65573, 67845, 131858, 65574, 66566, 131344, 65567, 66822, 65812, 66064,
-    65571, 67078, 65813, 66320, 65572, 67334, 131604, 65576, 67590, 66069, 66324, 65577,
-    67846, 131861, 65578, 66567, 131345, 65568, 66823, 65813, 66065, 65572, 67079, 65814,
-    66321, 65573, 67335, 131605, 65577, 67591, 66070, 66325, 65578, 67847, 131862, 65579,
-    66568, 131346, 65569, 66824, 65814, 66066, 65573, 67080, 65815, 66322, 65574, 67336,
-    131606, 65578, 67592, 66071, 66326, 65579, 67848, 131863, 65580, 66569, 131347, 65570,
-    66825, 65815, 66067, 65574, 67081, 65816, 66323, 65575, 67337, 131607, 65579, 67593,
-    66072, 66327, 65580, 67849, 131864, 65581,
-};
-__device__ const uint16_t kKetOff_fdfp[31] = {
-    0, 2, 4, 6, 8, 10, 12, 14, 16, 18, 20, 22,
-    24, 26, 28, 30, 32, 34, 36, 38, 40, 42, 44, 46,
-    48, 50, 52, 54, 56, 58, 60,
-};
-__device__ const uint32_t kKetTerm_fdfp[60] = {
-    65792, 65546, 66048, 65547, 66304, 65548, 65793, 65547, 66049, 65549, 66305, 65550,
-    65794, 65548, 66050, 65550, 66306, 65551, 65795, 65549, 66051, 65552, 66307, 65553,
-    65796, 65551, 66052, 65554, 66308, 65555, 65797, 65550, 66053, 65553, 66309, 65554,
-    65798, 65552, 66054, 65556, 66310, 65557, 65799, 65553, 66055, 65557, 66311, 65558,
-    65800, 65554, 66056, 65558, 66312, 65559, 65801, 65555, 66057, 65559, 66313, 65560,
-};
 __device__ const double kNormAB_fdfp[60] = {
     0.14907119849998599, 0.2581988897471611, 0.2581988897471611, 0.14907119849998599,
     0.2581988897471611, 0.14907119849998599, 0.3333333333333334, 0.5773502691896258,
@@ -225,24 +339,12 @@ __device__ const double kNormAB_fdfp[60] = {
     0.5773502691896258, 0.3333333333333334, 0.14907119849998599, 0.2581988897471611,
     0.2581988897471611, 0.14907119849998599, 0.2581988897471611, 0.14907119849998599,
 };
-__device__ const double kNormCD_fdfp[30] = {
-    0.2581988897471611, 0.2581988897471611, 0.2581988897471611, 0.5773502691896258,
-    0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
-    0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
-    0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 1.0,
-    1.0, 1.0, 0.2581988897471611, 0.2581988897471611,
-    0.2581988897471611, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
-    0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.2581988897471611,
-    0.2581988897471611, 0.2581988897471611,
-};
-
 
 // column components cx | cy << 4 | cz << 8
 __device__ const uint16_t kCol_fdfp[25] = { 3, 18, 258, 33, 513, 273, 48, 288, 528, 768, 4, 19, 259, 34, 274, 514, 49, 289, 529, 769, 64, 304, 544, 784, 1024 };
 
 __device__ __forceinline__ RysClassTabs tabs_fdfp() {
-    return RysClassTabs{kBlk_fdfp, kBraOff_fdfp, kBraTerm_fdfp, kKetOff_fdfp, kKetTerm_fdfp,
-                        kNormAB_fdfp, kNormCD_fdfp, kCol_fdfp};
+    return RysClassTabs{kNormAB_fdfp, kCol_fdfp};
 }
 
 template <int MIXED>
@@ -255,8 +357,8 @@ static void rys_prepare_fdfp() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_fdfp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 87680);
-        cudaFuncSetAttribute(rys_queue_fdfp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 87680);
+        cudaFuncSetAttribute(rys_queue_fdfp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 107520);
+        cudaFuncSetAttribute(rys_queue_fdfp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 107520);
 
         done[dev] = true;
     }
@@ -268,16 +370,16 @@ void launch_rys_fdfp(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_fdfp();
     constexpr int ng = 128 / C_fdfp::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_fdfp<1><<<grid, 128, 87680, s>>>(Q, R);
-    else rys_queue_fdfp<0><<<grid, 128, 87680, s>>>(Q, R);
+    if (mixed) rys_queue_fdfp<1><<<grid, 128, 107520, s>>>(Q, R);
+    else rys_queue_fdfp<0><<<grid, 128, 107520, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_fdfp(int mixed) {
     rys_prepare_fdfp();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fdfp<1>, 128, 87680);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fdfp<0>, 128, 87680);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fdfp<1>, 128, 107520);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fdfp<0>, 128, 107520);
     return n;
 }
 

@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (fd|fs).  Do not edit.
-// roots 5, block 46 x 10, outputs 60 x 10, group 64 threads,
-// 12 primitive quartets per batch, 1 slot(s), 8 accumulators per thread, 69760 B shared per block.
+// roots 5, block 46 x 10, outputs 60 x 10, group 32 threads, 1 ket pairs a round,
+// 4 primitive quartets per ket pair and batch, 46720 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,91 +11,267 @@ struct C_fdfs {
     static constexpr int NA = 46, NC = 10, NBLK = 460;
     static constexpr int NB = 6, ND = 1;
     static constexpr int NAB = 60, NCD = 10;
-    static constexpr int G = 64, NPB = 12, NSLOT = 1, ACC = 8;
-    static constexpr int S = 24;
-    static constexpr int SMEM_GROUP = 4360;
-    static constexpr bool COL = false;
+    static constexpr int G = 32, W = 1, H = 1, PB = 4;
+    static constexpr int S = 24, SI = 73, NCP = 11, NCDP = 11;
+    static constexpr int SMEM_GROUP = 1460;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
-    __device__ __forceinline__ static void col_update(const T *, const T *, const T *, A *) {}
+    __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
+        acc[0] = fma(x[3] * y[0], z[0], acc[0]);
+        acc[1] = fma(x[2] * y[1], z[0], acc[1]);
+        acc[2] = fma(x[2] * y[0], z[1], acc[2]);
+        acc[3] = fma(x[1] * y[2], z[0], acc[3]);
+        acc[4] = fma(x[1] * y[0], z[2], acc[4]);
+        acc[5] = fma(x[1] * y[1], z[1], acc[5]);
+        acc[6] = fma(x[0] * y[3], z[0], acc[6]);
+        acc[7] = fma(x[0] * y[2], z[1], acc[7]);
+        acc[8] = fma(x[0] * y[1], z[2], acc[8]);
+        acc[9] = fma(x[0] * y[0], z[3], acc[9]);
+        acc[10] = fma(x[4] * y[0], z[0], acc[10]);
+        acc[11] = fma(x[3] * y[1], z[0], acc[11]);
+        acc[12] = fma(x[3] * y[0], z[1], acc[12]);
+        acc[13] = fma(x[2] * y[2], z[0], acc[13]);
+        acc[14] = fma(x[2] * y[1], z[1], acc[14]);
+        acc[15] = fma(x[2] * y[0], z[2], acc[15]);
+        acc[16] = fma(x[1] * y[3], z[0], acc[16]);
+        acc[17] = fma(x[1] * y[2], z[1], acc[17]);
+        acc[18] = fma(x[1] * y[1], z[2], acc[18]);
+        acc[19] = fma(x[1] * y[0], z[3], acc[19]);
+        acc[20] = fma(x[0] * y[4], z[0], acc[20]);
+        acc[21] = fma(x[0] * y[3], z[1], acc[21]);
+        acc[22] = fma(x[0] * y[2], z[2], acc[22]);
+        acc[23] = fma(x[0] * y[1], z[3], acc[23]);
+        acc[24] = fma(x[0] * y[0], z[4], acc[24]);
+        acc[25] = fma(x[5] * y[0], z[0], acc[25]);
+        acc[26] = fma(x[4] * y[1], z[0], acc[26]);
+        acc[27] = fma(x[4] * y[0], z[1], acc[27]);
+        acc[28] = fma(x[3] * y[2], z[0], acc[28]);
+        acc[29] = fma(x[3] * y[1], z[1], acc[29]);
+        acc[30] = fma(x[3] * y[0], z[2], acc[30]);
+        acc[31] = fma(x[2] * y[3], z[0], acc[31]);
+        acc[32] = fma(x[2] * y[2], z[1], acc[32]);
+        acc[33] = fma(x[2] * y[1], z[2], acc[33]);
+        acc[34] = fma(x[2] * y[0], z[3], acc[34]);
+        acc[35] = fma(x[1] * y[4], z[0], acc[35]);
+        acc[36] = fma(x[1] * y[3], z[1], acc[36]);
+        acc[37] = fma(x[1] * y[2], z[2], acc[37]);
+        acc[38] = fma(x[1] * y[1], z[3], acc[38]);
+        acc[39] = fma(x[1] * y[0], z[4], acc[39]);
+        acc[40] = fma(x[0] * y[5], z[0], acc[40]);
+        acc[41] = fma(x[0] * y[4], z[1], acc[41]);
+        acc[42] = fma(x[0] * y[3], z[2], acc[42]);
+        acc[43] = fma(x[0] * y[2], z[3], acc[43]);
+        acc[44] = fma(x[0] * y[1], z[4], acc[44]);
+        acc[45] = fma(x[0] * y[0], z[5], acc[45]);
+    }
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[10], in[25]);
+        const double h1 = fma(x, in[0], in[10]);
+        const double h2 = fma(x, h1, h0);
+        const double h3 = fma(y, in[10], in[26]);
+        const double h4 = fma(y, in[0], in[11]);
+        const double h5 = fma(x, h4, h3);
+        const double h6 = fma(z, in[10], in[27]);
+        const double h7 = fma(z, in[0], in[12]);
+        const double h8 = fma(x, h7, h6);
+        const double h9 = fma(y, in[11], in[28]);
+        const double h10 = fma(y, h4, h9);
+        const double h11 = fma(z, in[11], in[29]);
+        const double h12 = fma(y, h7, h11);
+        const double h13 = fma(z, in[12], in[30]);
+        const double h14 = fma(z, h7, h13);
+        const double h15 = fma(x, in[11], in[26]);
+        const double h16 = fma(x, in[1], in[11]);
+        const double h17 = fma(x, h16, h15);
+        const double h18 = fma(y, in[1], in[13]);
+        const double h19 = fma(x, h18, h9);
+        const double h20 = fma(z, in[1], in[14]);
+        const double h21 = fma(x, h20, h11);
+        const double h22 = fma(y, in[13], in[31]);
+        const double h23 = fma(y, h18, h22);
+        const double h24 = fma(z, in[13], in[32]);
+        const double h25 = fma(y, h20, h24);
+        const double h26 = fma(z, in[14], in[33]);
+        const double h27 = fma(z, h20, h26);
+        const double h28 = fma(x, in[12], in[27]);
+        const double h29 = fma(x, in[2], in[12]);
+        const double h30 = fma(x, h29, h28);
+        const double h31 = fma(y, in[12], in[29]);
+        const double h32 = fma(y, in[2], in[14]);
+        const double h33 = fma(x, h32, h31);
+        const double h34 = fma(z, in[2], in[15]);
+        const double h35 = fma(x, h34, h13);
+        const double h36 = fma(y, in[14], in[32]);
+        const double h37 = fma(y, h32, h36);
+        const double h38 = fma(y, h34, h26);
+        const double h39 = fma(z, in[15], in[34]);
+        const double h40 = fma(z, h34, h39);
+        const double h41 = fma(x, in[13], in[28]);
+        const double h42 = fma(x, in[3], in[13]);
+        const double h43 = fma(x, h42, h41);
+        const double h44 = fma(y, in[3], in[16]);
+        const double h45 = fma(x, h44, h22);
+        const double h46 = fma(z, in[3], in[17]);
+        const double h47 = fma(x, h46, h24);
+        const double h48 = fma(y, in[16], in[35]);
+        const double h49 = fma(y, h44, h48);
+        const double h50 = fma(z, in[16], in[36]);
+        const double h51 = fma(y, h46, h50);
+        const double h52 = fma(z, in[17], in[37]);
+        const double h53 = fma(z, h46, h52);
+        const double h54 = fma(x, in[15], in[30]);
+        const double h55 = fma(x, in[4], in[15]);
+        const double h56 = fma(x, h55, h54);
+        const double h57 = fma(y, in[15], in[33]);
+        const double h58 = fma(y, in[4], in[18]);
+        const double h59 = fma(x, h58, h57);
+        const double h60 = fma(z, in[4], in[19]);
+        const double h61 = fma(x, h60, h39);
+        const double h62 = fma(y, in[18], in[37]);
+        const double h63 = fma(y, h58, h62);
+        const double h64 = fma(z, in[18], in[38]);
+        const double h65 = fma(y, h60, h64);
+        const double h66 = fma(z, in[19], in[39]);
+        const double h67 = fma(z, h60, h66);
+        const double h68 = fma(x, in[14], in[29]);
+        const double h69 = fma(x, in[5], in[14]);
+        const double h70 = fma(x, h69, h68);
+        const double h71 = fma(y, in[5], in[17]);
+        const double h72 = fma(x, h71, h36);
+        const double h73 = fma(z, in[5], in[18]);
+        const double h74 = fma(x, h73, h26);
+        const double h75 = fma(y, in[17], in[36]);
+        const double h76 = fma(y, h71, h75);
+        const double h77 = fma(y, h73, h52);
+        const double h78 = fma(z, h73, h64);
+        const double h79 = fma(x, in[16], in[31]);
+        const double h80 = fma(x, in[6], in[16]);
+        const double h81 = fma(x, h80, h79);
+        const double h82 = fma(y, in[6], in[20]);
+        const double h83 = fma(x, h82, h48);
+        const double h84 = fma(z, in[6], in[21]);
+        const double h85 = fma(x, h84, h50);
+        const double h86 = fma(y, in[20], in[40]);
+        const double h87 = fma(y, h82, h86);
+        const double h88 = fma(z, in[20], in[41]);
+        const double h89 = fma(y, h84, h88);
+        const double h90 = fma(z, in[21], in[42]);
+        const double h91 = fma(z, h84, h90);
+        const double h92 = fma(x, in[17], in[32]);
+        const double h93 = fma(x, in[7], in[17]);
+        const double h94 = fma(x, h93, h92);
+        const double h95 = fma(y, in[7], in[21]);
+        const double h96 = fma(x, h95, h75);
+        const double h97 = fma(z, in[7], in[22]);
+        const double h98 = fma(x, h97, h52);
+        const double h99 = fma(y, in[21], in[41]);
+        const double h100 = fma(y, h95, h99);
+        const double h101 = fma(y, h97, h90);
+        const double h102 = fma(z, in[22], in[43]);
+        const double h103 = fma(z, h97, h102);
+        const double h104 = fma(x, in[18], in[33]);
+        const double h105 = fma(x, in[8], in[18]);
+        const double h106 = fma(x, h105, h104);
+        const double h107 = fma(y, in[8], in[22]);
+        const double h108 = fma(x, h107, h62);
+        const double h109 = fma(z, in[8], in[23]);
+        const double h110 = fma(x, h109, h64);
+        const double h111 = fma(y, in[22], in[42]);
+        const double h112 = fma(y, h107, h111);
+        const double h113 = fma(y, h109, h102);
+        const double h114 = fma(z, in[23], in[44]);
+        const double h115 = fma(z, h109, h114);
+        const double h116 = fma(x, in[19], in[34]);
+        const double h117 = fma(x, in[9], in[19]);
+        const double h118 = fma(x, h117, h116);
+        const double h119 = fma(y, in[19], in[38]);
+        const double h120 = fma(y, in[9], in[23]);
+        const double h121 = fma(x, h120, h119);
+        const double h122 = fma(z, in[9], in[24]);
+        const double h123 = fma(x, h122, h66);
+        const double h124 = fma(y, in[23], in[43]);
+        const double h125 = fma(y, h120, h124);
+        const double h126 = fma(y, h122, h114);
+        const double h127 = fma(z, in[24], in[45]);
+        const double h128 = fma(z, h122, h127);
+        out[0] = h2;
+        out[11] = h5;
+        out[22] = h8;
+        out[33] = h10;
+        out[44] = h12;
+        out[55] = h14;
+        out[66] = h17;
+        out[77] = h19;
+        out[88] = h21;
+        out[99] = h23;
+        out[110] = h25;
+        out[121] = h27;
+        out[132] = h30;
+        out[143] = h33;
+        out[154] = h35;
+        out[165] = h37;
+        out[176] = h38;
+        out[187] = h40;
+        out[198] = h43;
+        out[209] = h45;
+        out[220] = h47;
+        out[231] = h49;
+        out[242] = h51;
+        out[253] = h53;
+        out[264] = h56;
+        out[275] = h59;
+        out[286] = h61;
+        out[297] = h63;
+        out[308] = h65;
+        out[319] = h67;
+        out[330] = h70;
+        out[341] = h72;
+        out[352] = h74;
+        out[363] = h76;
+        out[374] = h77;
+        out[385] = h78;
+        out[396] = h81;
+        out[407] = h83;
+        out[418] = h85;
+        out[429] = h87;
+        out[440] = h89;
+        out[451] = h91;
+        out[462] = h94;
+        out[473] = h96;
+        out[484] = h98;
+        out[495] = h100;
+        out[506] = h101;
+        out[517] = h103;
+        out[528] = h106;
+        out[539] = h108;
+        out[550] = h110;
+        out[561] = h112;
+        out[572] = h113;
+        out[583] = h115;
+        out[594] = h118;
+        out[605] = h121;
+        out[616] = h123;
+        out[627] = h125;
+        out[638] = h126;
+        out[649] = h128;
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        out[0] = in[0] * (nrm * 0.2581988897471611);
+        out[1] = in[1] * (nrm * 0.5773502691896258);
+        out[2] = in[2] * (nrm * 0.5773502691896258);
+        out[3] = in[3] * (nrm * 0.5773502691896258);
+        out[4] = in[4] * (nrm * 0.5773502691896258);
+        out[5] = in[5] * (nrm * 1.0);
+        out[6] = in[6] * (nrm * 0.2581988897471611);
+        out[7] = in[7] * (nrm * 0.5773502691896258);
+        out[8] = in[8] * (nrm * 0.5773502691896258);
+        out[9] = in[9] * (nrm * 0.2581988897471611);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_fdfs[460] = {
-    15, 270, 65550, 525, 131085, 65805, 780, 66060, 131340, 196620, 1035, 1290,
-    66570, 1545, 132105, 66825, 1800, 67080, 132360, 197640, 262155, 262410, 327690, 262665,
-    393225, 327945, 262920, 328200, 393480, 458760, 2055, 2310, 67590, 2565, 133125, 67845,
-    2820, 68100, 133380, 198660, 524295, 524550, 589830, 524805, 655365, 590085, 525060, 590340,
-    655620, 720900, 263175, 263430, 328710, 263685, 394245, 328965, 263940, 329220, 394500, 459780,
-    3075, 3330, 68610, 3585, 134145, 68865, 3840, 69120, 134400, 199680, 264195, 264450,
-    329730, 264705, 395265, 329985, 264960, 330240, 395520, 460800, 525315, 525570, 590850, 525825,
-    656385, 591105, 526080, 591360, 656640, 721920, 786435, 786690, 851970, 786945, 917505, 852225,
-    787200, 852480, 917760, 983040, 19, 274, 65554, 529, 131089, 65809, 784, 66064,
-    131344, 196624, 1039, 1294, 66574, 1549, 132109, 66829, 1804, 67084, 132364, 197644,
-    262159, 262414, 327694, 262669, 393229, 327949, 262924, 328204, 393484, 458764, 2059, 2314,
-    67594, 2569, 133129, 67849, 2824, 68104, 133384, 198664, 263179, 263434, 328714, 263689,
-    394249, 328969, 263944, 329224, 394504, 459784, 524299, 524554, 589834, 524809, 655369, 590089,
-    525064, 590344, 655624, 720904, 3079, 3334, 68614, 3589, 134149, 68869, 3844, 69124,
-    134404, 199684, 264199, 264454, 329734, 264709, 395269, 329989, 264964, 330244, 395524, 460804,
-    525319, 525574, 590854, 525829, 656389, 591109, 526084, 591364, 656644, 721924, 786439, 786694,
-    851974, 786949, 917509, 852229, 787204, 852484, 917764, 983044, 4099, 4354, 69634, 4609,
-    135169, 69889, 4864, 70144, 135424, 200704, 265219, 265474, 330754, 265729, 396289, 331009,
-    265984, 331264, 396544, 461824, 526339, 526594, 591874, 526849, 657409, 592129, 527104, 592384,
-    657664, 722944, 787459, 787714, 852994, 787969, 918529, 853249, 788224, 853504, 918784, 984064,
-    1048579, 1048834, 1114114, 1049089, 1179649, 1114369, 1049344, 1114624, 1179904, 1245184, 23, 278,
-    65558, 533, 131093, 65813, 788, 66068, 131348, 196628, 1043, 1298, 66578, 1553,
-    132113, 66833, 1808, 67088, 132368, 197648, 262163, 262418, 327698, 262673, 393233, 327953,
-    262928, 328208, 393488, 458768, 2063, 2318, 67598, 2573, 133133, 67853, 2828, 68108,
-    133388, 198668, 263183, 263438, 328718, 263693, 394253, 328973, 263948, 329228, 394508, 459788,
-    524303, 524558, 589838, 524813, 655373, 590093, 525068, 590348, 655628, 720908, 3083, 3338,
-    68618, 3593, 134153, 68873, 3848, 69128, 134408, 199688, 264203, 264458, 329738, 264713,
-    395273, 329993, 264968, 330248, 395528, 460808, 525323, 525578, 590858, 525833, 656393, 591113,
-    526088, 591368, 656648, 721928, 786443, 786698, 851978, 786953, 917513, 852233, 787208, 852488,
-    917768, 983048, 4103, 4358, 69638, 4613, 135173, 69893, 4868, 70148, 135428, 200708,
-    265223, 265478, 330758, 265733, 396293, 331013, 265988, 331268, 396548, 461828, 526343, 526598,
-    591878, 526853, 657413, 592133, 527108, 592388, 657668, 722948, 787463, 787718, 852998, 787973,
-    918533, 853253, 788228, 853508, 918788, 984068, 1048583, 1048838, 1114118, 1049093, 1179653, 1114373,
-    1049348, 1114628, 1179908, 1245188, 5123, 5378, 70658, 5633, 136193, 70913, 5888, 71168,
-    136448, 201728, 266243, 266498, 331778, 266753, 397313, 332033, 267008, 332288, 397568, 462848,
-    527363, 527618, 592898, 527873, 658433, 593153, 528128, 593408, 658688, 723968, 788483, 788738,
-    854018, 788993, 919553, 854273, 789248, 854528, 919808, 985088, 1049603, 1049858, 1115138, 1050113,
-    1180673, 1115393, 1050368, 1115648, 1180928, 1246208, 1310723, 1310978, 1376258, 1311233, 1441793, 1376513,
-    1311488, 1376768, 1442048, 1507328,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_fdfs[61] = {
-    0, 3, 7, 11, 14, 18, 21, 24, 28, 32, 35, 39,
-    42, 45, 49, 53, 56, 60, 63, 66, 70, 74, 77, 81,
-    84, 87, 91, 95, 98, 102, 105, 108, 112, 116, 119, 123,
-    126, 129, 133, 137, 140, 144, 147, 150, 154, 158, 161, 165,
-    168, 171, 175, 179, 182, 186, 189, 192, 196, 200, 203, 207,
-    210,
-};
-__device__ const uint32_t kBraTerm_fdfs[210] = {
-    66560, 131338, 65561, 66816, 65803, 66058, 65562, 67072, 65804, 66314, 65563, 67328,
-    131595, 65564, 67584, 66060, 66315, 65565, 67840, 131852, 65566, 66561, 131339, 65562,
-    66817, 65805, 66059, 65564, 67073, 65806, 66315, 65565, 67329, 131597, 65567, 67585,
-    66062, 66317, 65568, 67841, 131854, 65569, 66562, 131340, 65563, 66818, 65806, 66060,
-    65565, 67074, 65807, 66316, 65566, 67330, 131598, 65568, 67586, 66063, 66318, 65569,
-    67842, 131855, 65570, 66563, 131341, 65564, 66819, 65808, 66061, 65567, 67075, 65809,
-    66317, 65568, 67331, 131600, 65571, 67587, 66065, 66320, 65572, 67843, 131857, 65573,
-    66564, 131343, 65566, 66820, 65810, 66063, 65569, 67076, 65811, 66319, 65570, 67332,
-    131602, 65573, 67588, 66067, 66322, 65574, 67844, 131859, 65575, 66565, 131342, 65565,
-    66821, 65809, 66062, 65568, 67077, 65810, 66318, 65569, 67333, 131601, 65572, 67589,
-    66066, 66321, 65573, 67845, 131858, 65574, 66566, 131344, 65567, 66822, 65812, 66064,
-    65571, 67078, 65813, 66320, 65572, 67334, 131604, 65576, 67590, 66069, 66324, 65577,
-    67846, 131861, 65578, 66567, 131345, 65568, 66823, 65813, 66065, 65572, 67079, 65814,
-    66321, 65573, 67335, 131605, 65577, 67591, 66070, 66325, 65578, 67847, 131862, 65579,
-    66568, 131346, 65569, 66824, 65814, 66066, 65573, 67080, 65815, 66322, 65574, 67336,
-    131606, 65578, 67592, 66071, 66326, 65579, 67848, 131863, 65580, 66569, 131347, 65570,
-    66825, 65815, 66067, 65574, 67081, 65816, 66323, 65575, 67337, 131607, 65579, 67593,
-    66072, 66327, 65580, 67849, 131864, 65581,
-};
-__device__ const uint16_t kKetOff_fdfs[11] = {
-    0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10,
-};
-__device__ const uint32_t kKetTerm_fdfs[10] = {
-    65536, 65537, 65538, 65539, 65540, 65541, 65542, 65543, 65544, 65545,
-};
 __device__ const double kNormAB_fdfs[60] = {
     0.14907119849998599, 0.2581988897471611, 0.2581988897471611, 0.14907119849998599,
     0.2581988897471611, 0.14907119849998599, 0.3333333333333334, 0.5773502691896258,
@@ -113,16 +289,12 @@ __device__ const double kNormAB_fdfs[60] = {
     0.5773502691896258, 0.3333333333333334, 0.14907119849998599, 0.2581988897471611,
     0.2581988897471611, 0.14907119849998599, 0.2581988897471611, 0.14907119849998599,
 };
-__device__ const double kNormCD_fdfs[10] = {
-    0.2581988897471611, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
-    0.5773502691896258, 1.0, 0.2581988897471611, 0.5773502691896258,
-    0.5773502691896258, 0.2581988897471611,
-};
 
+// column components cx | cy << 4 | cz << 8
+__device__ const uint16_t kCol_fdfs[10] = { 3, 18, 258, 33, 513, 273, 48, 288, 528, 768 };
 
 __device__ __forceinline__ RysClassTabs tabs_fdfs() {
-    return RysClassTabs{kBlk_fdfs, kBraOff_fdfs, kBraTerm_fdfs, kKetOff_fdfs, kKetTerm_fdfs,
-                        kNormAB_fdfs, kNormCD_fdfs, nullptr};
+    return RysClassTabs{kNormAB_fdfs, kCol_fdfs};
 }
 
 template <int MIXED>
@@ -135,8 +307,8 @@ static void rys_prepare_fdfs() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_fdfs<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 69760);
-        cudaFuncSetAttribute(rys_queue_fdfs<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 69760);
+        cudaFuncSetAttribute(rys_queue_fdfs<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 46720);
+        cudaFuncSetAttribute(rys_queue_fdfs<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 46720);
 
         done[dev] = true;
     }
@@ -148,16 +320,16 @@ void launch_rys_fdfs(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_fdfs();
     constexpr int ng = 128 / C_fdfs::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_fdfs<1><<<grid, 128, 69760, s>>>(Q, R);
-    else rys_queue_fdfs<0><<<grid, 128, 69760, s>>>(Q, R);
+    if (mixed) rys_queue_fdfs<1><<<grid, 128, 46720, s>>>(Q, R);
+    else rys_queue_fdfs<0><<<grid, 128, 46720, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_fdfs(int mixed) {
     rys_prepare_fdfs();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fdfs<1>, 128, 69760);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fdfs<0>, 128, 69760);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fdfs<1>, 128, 46720);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fdfs<0>, 128, 46720);
     return n;
 }
 

@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (ff|fp).  Do not edit.
-// roots 6, block 74 x 25, outputs 100 x 30, group 128 threads,
-// 9 primitive quartets per batch, 1 slot(s), 15 accumulators per thread, 45680 B shared per block.
+// roots 6, block 74 x 25, outputs 100 x 30, group 32 threads, 1 ket pairs a round,
+// 5 primitive quartets per ket pair and batch, 179200 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,245 +11,607 @@ struct C_fffp {
     static constexpr int NA = 74, NC = 25, NBLK = 1850;
     static constexpr int NB = 10, ND = 3;
     static constexpr int NAB = 100, NCD = 30;
-    static constexpr int G = 128, NPB = 9, NSLOT = 1, ACC = 15;
-    static constexpr int S = 35;
-    static constexpr int SMEM_GROUP = 5710;
-    static constexpr bool COL = false;
+    static constexpr int G = 32, W = 1, H = 1, PB = 5;
+    static constexpr int S = 35, SI = 105, NCP = 25, NCDP = 31;
+    static constexpr int SMEM_GROUP = 5600;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
-    __device__ __forceinline__ static void col_update(const T *, const T *, const T *, A *) {}
+    __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
+        acc[0] = fma(x[3] * y[0], z[0], acc[0]);
+        acc[1] = fma(x[2] * y[1], z[0], acc[1]);
+        acc[2] = fma(x[2] * y[0], z[1], acc[2]);
+        acc[3] = fma(x[1] * y[2], z[0], acc[3]);
+        acc[4] = fma(x[1] * y[0], z[2], acc[4]);
+        acc[5] = fma(x[1] * y[1], z[1], acc[5]);
+        acc[6] = fma(x[0] * y[3], z[0], acc[6]);
+        acc[7] = fma(x[0] * y[2], z[1], acc[7]);
+        acc[8] = fma(x[0] * y[1], z[2], acc[8]);
+        acc[9] = fma(x[0] * y[0], z[3], acc[9]);
+        acc[10] = fma(x[4] * y[0], z[0], acc[10]);
+        acc[11] = fma(x[3] * y[1], z[0], acc[11]);
+        acc[12] = fma(x[3] * y[0], z[1], acc[12]);
+        acc[13] = fma(x[2] * y[2], z[0], acc[13]);
+        acc[14] = fma(x[2] * y[1], z[1], acc[14]);
+        acc[15] = fma(x[2] * y[0], z[2], acc[15]);
+        acc[16] = fma(x[1] * y[3], z[0], acc[16]);
+        acc[17] = fma(x[1] * y[2], z[1], acc[17]);
+        acc[18] = fma(x[1] * y[1], z[2], acc[18]);
+        acc[19] = fma(x[1] * y[0], z[3], acc[19]);
+        acc[20] = fma(x[0] * y[4], z[0], acc[20]);
+        acc[21] = fma(x[0] * y[3], z[1], acc[21]);
+        acc[22] = fma(x[0] * y[2], z[2], acc[22]);
+        acc[23] = fma(x[0] * y[1], z[3], acc[23]);
+        acc[24] = fma(x[0] * y[0], z[4], acc[24]);
+        acc[25] = fma(x[5] * y[0], z[0], acc[25]);
+        acc[26] = fma(x[4] * y[1], z[0], acc[26]);
+        acc[27] = fma(x[4] * y[0], z[1], acc[27]);
+        acc[28] = fma(x[3] * y[2], z[0], acc[28]);
+        acc[29] = fma(x[3] * y[1], z[1], acc[29]);
+        acc[30] = fma(x[3] * y[0], z[2], acc[30]);
+        acc[31] = fma(x[2] * y[3], z[0], acc[31]);
+        acc[32] = fma(x[2] * y[2], z[1], acc[32]);
+        acc[33] = fma(x[2] * y[1], z[2], acc[33]);
+        acc[34] = fma(x[2] * y[0], z[3], acc[34]);
+        acc[35] = fma(x[1] * y[4], z[0], acc[35]);
+        acc[36] = fma(x[1] * y[3], z[1], acc[36]);
+        acc[37] = fma(x[1] * y[2], z[2], acc[37]);
+        acc[38] = fma(x[1] * y[1], z[3], acc[38]);
+        acc[39] = fma(x[1] * y[0], z[4], acc[39]);
+        acc[40] = fma(x[0] * y[5], z[0], acc[40]);
+        acc[41] = fma(x[0] * y[4], z[1], acc[41]);
+        acc[42] = fma(x[0] * y[3], z[2], acc[42]);
+        acc[43] = fma(x[0] * y[2], z[3], acc[43]);
+        acc[44] = fma(x[0] * y[1], z[4], acc[44]);
+        acc[45] = fma(x[0] * y[0], z[5], acc[45]);
+        acc[46] = fma(x[6] * y[0], z[0], acc[46]);
+        acc[47] = fma(x[5] * y[1], z[0], acc[47]);
+        acc[48] = fma(x[5] * y[0], z[1], acc[48]);
+        acc[49] = fma(x[4] * y[2], z[0], acc[49]);
+        acc[50] = fma(x[4] * y[1], z[1], acc[50]);
+        acc[51] = fma(x[4] * y[0], z[2], acc[51]);
+        acc[52] = fma(x[3] * y[3], z[0], acc[52]);
+        acc[53] = fma(x[3] * y[2], z[1], acc[53]);
+        acc[54] = fma(x[3] * y[1], z[2], acc[54]);
+        acc[55] = fma(x[3] * y[0], z[3], acc[55]);
+        acc[56] = fma(x[2] * y[4], z[0], acc[56]);
+        acc[57] = fma(x[2] * y[3], z[1], acc[57]);
+        acc[58] = fma(x[2] * y[2], z[2], acc[58]);
+        acc[59] = fma(x[2] * y[1], z[3], acc[59]);
+        acc[60] = fma(x[2] * y[0], z[4], acc[60]);
+        acc[61] = fma(x[1] * y[5], z[0], acc[61]);
+        acc[62] = fma(x[1] * y[4], z[1], acc[62]);
+        acc[63] = fma(x[1] * y[3], z[2], acc[63]);
+        acc[64] = fma(x[1] * y[2], z[3], acc[64]);
+        acc[65] = fma(x[1] * y[1], z[4], acc[65]);
+        acc[66] = fma(x[1] * y[0], z[5], acc[66]);
+        acc[67] = fma(x[0] * y[6], z[0], acc[67]);
+        acc[68] = fma(x[0] * y[5], z[1], acc[68]);
+        acc[69] = fma(x[0] * y[4], z[2], acc[69]);
+        acc[70] = fma(x[0] * y[3], z[3], acc[70]);
+        acc[71] = fma(x[0] * y[2], z[4], acc[71]);
+        acc[72] = fma(x[0] * y[1], z[5], acc[72]);
+        acc[73] = fma(x[0] * y[0], z[6], acc[73]);
+    }
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[25], in[46]);
+        const double h1 = fma(x, in[10], in[25]);
+        const double h2 = fma(x, h1, h0);
+        const double h3 = fma(x, in[0], in[10]);
+        const double h4 = fma(x, h3, h1);
+        const double h5 = fma(x, h4, h2);
+        const double h6 = fma(y, in[25], in[47]);
+        const double h7 = fma(y, in[10], in[26]);
+        const double h8 = fma(x, h7, h6);
+        const double h9 = fma(y, in[0], in[11]);
+        const double h10 = fma(x, h9, h7);
+        const double h11 = fma(x, h10, h8);
+        const double h12 = fma(z, in[25], in[48]);
+        const double h13 = fma(z, in[10], in[27]);
+        const double h14 = fma(x, h13, h12);
+        const double h15 = fma(z, in[0], in[12]);
+        const double h16 = fma(x, h15, h13);
+        const double h17 = fma(x, h16, h14);
+        const double h18 = fma(y, in[26], in[49]);
+        const double h19 = fma(y, in[11], in[28]);
+        const double h20 = fma(x, h19, h18);
+        const double h21 = fma(y, h10, h20);
+        const double h22 = fma(z, in[27], in[51]);
+        const double h23 = fma(z, in[12], in[30]);
+        const double h24 = fma(x, h23, h22);
+        const double h25 = fma(z, h16, h24);
+        const double h26 = fma(z, in[26], in[50]);
+        const double h27 = fma(y, h13, h26);
+        const double h28 = fma(z, in[11], in[29]);
+        const double h29 = fma(y, h15, h28);
+        const double h30 = fma(x, h29, h27);
+        const double h31 = fma(y, in[28], in[52]);
+        const double h32 = fma(y, h19, h31);
+        const double h33 = fma(y, h9, h19);
+        const double h34 = fma(y, h33, h32);
+        const double h35 = fma(z, in[28], in[53]);
+        const double h36 = fma(y, h28, h35);
+        const double h37 = fma(y, h29, h36);
+        const double h38 = fma(z, in[29], in[54]);
+        const double h39 = fma(y, h23, h38);
+        const double h40 = fma(z, h29, h39);
+        const double h41 = fma(z, in[30], in[55]);
+        const double h42 = fma(z, h23, h41);
+        const double h43 = fma(z, h15, h23);
+        const double h44 = fma(z, h43, h42);
+        const double h45 = fma(x, in[26], in[47]);
+        const double h46 = fma(x, in[11], in[26]);
+        const double h47 = fma(x, h46, h45);
+        const double h48 = fma(x, in[1], in[11]);
+        const double h49 = fma(x, h48, h46);
+        const double h50 = fma(x, h49, h47);
+        const double h51 = fma(y, in[1], in[13]);
+        const double h52 = fma(x, h51, h19);
+        const double h53 = fma(x, h52, h20);
+        const double h54 = fma(x, h28, h26);
+        const double h55 = fma(z, in[1], in[14]);
+        const double h56 = fma(x, h55, h28);
+        const double h57 = fma(x, h56, h54);
+        const double h58 = fma(y, in[13], in[31]);
+        const double h59 = fma(x, h58, h31);
+        const double h60 = fma(y, h52, h59);
+        const double h61 = fma(z, in[14], in[33]);
+        const double h62 = fma(x, h61, h38);
+        const double h63 = fma(z, h56, h62);
+        const double h64 = fma(z, in[13], in[32]);
+        const double h65 = fma(y, h55, h64);
+        const double h66 = fma(x, h65, h36);
+        const double h67 = fma(y, in[31], in[56]);
+        const double h68 = fma(y, h58, h67);
+        const double h69 = fma(y, h51, h58);
+        const double h70 = fma(y, h69, h68);
+        const double h71 = fma(z, in[31], in[57]);
+        const double h72 = fma(y, h64, h71);
+        const double h73 = fma(y, h65, h72);
+        const double h74 = fma(z, in[32], in[58]);
+        const double h75 = fma(y, h61, h74);
+        const double h76 = fma(z, h65, h75);
+        const double h77 = fma(z, in[33], in[59]);
+        const double h78 = fma(z, h61, h77);
+        const double h79 = fma(z, h55, h61);
+        const double h80 = fma(z, h79, h78);
+        const double h81 = fma(x, in[27], in[48]);
+        const double h82 = fma(x, in[12], in[27]);
+        const double h83 = fma(x, h82, h81);
+        const double h84 = fma(x, in[2], in[12]);
+        const double h85 = fma(x, h84, h82);
+        const double h86 = fma(x, h85, h83);
+        const double h87 = fma(y, in[27], in[50]);
+        const double h88 = fma(y, in[12], in[29]);
+        const double h89 = fma(x, h88, h87);
+        const double h90 = fma(y, in[2], in[14]);
+        const double h91 = fma(x, h90, h88);
+        const double h92 = fma(x, h91, h89);
+        const double h93 = fma(z, in[2], in[15]);
+        const double h94 = fma(x, h93, h23);
+        const double h95 = fma(x, h94, h24);
+        const double h96 = fma(y, in[29], in[53]);
+        const double h97 = fma(y, in[14], in[32]);
+        const double h98 = fma(x, h97, h96);
+        const double h99 = fma(y, h91, h98);
+        const double h100 = fma(z, in[15], in[34]);
+        const double h101 = fma(x, h100, h41);
+        const double h102 = fma(z, h94, h101);
+        const double h103 = fma(y, h93, h61);
+        const double h104 = fma(x, h103, h39);
+        const double h105 = fma(y, in[32], in[57]);
+        const double h106 = fma(y, h97, h105);
+        const double h107 = fma(y, h90, h97);
+        const double h108 = fma(y, h107, h106);
+        const double h109 = fma(y, h103, h75);
+        const double h110 = fma(y, h100, h77);
+        const double h111 = fma(z, h103, h110);
+        const double h112 = fma(z, in[34], in[60]);
+        const double h113 = fma(z, h100, h112);
+        const double h114 = fma(z, h93, h100);
+        const double h115 = fma(z, h114, h113);
+        const double h116 = fma(x, in[28], in[49]);
+        const double h117 = fma(x, in[13], in[28]);
+        const double h118 = fma(x, h117, h116);
+        const double h119 = fma(x, in[3], in[13]);
+        const double h120 = fma(x, h119, h117);
+        const double h121 = fma(x, h120, h118);
+        const double h122 = fma(y, in[3], in[16]);
+        const double h123 = fma(x, h122, h58);
+        const double h124 = fma(x, h123, h59);
+        const double h125 = fma(x, h64, h35);
+        const double h126 = fma(z, in[3], in[17]);
+        const double h127 = fma(x, h126, h64);
+        const double h128 = fma(x, h127, h125);
+        const double h129 = fma(y, in[16], in[35]);
+        const double h130 = fma(x, h129, h67);
+        const double h131 = fma(y, h123, h130);
+        const double h132 = fma(z, in[17], in[37]);
+        const double h133 = fma(x, h132, h74);
+        const double h134 = fma(z, h127, h133);
+        const double h135 = fma(z, in[16], in[36]);
+        const double h136 = fma(y, h126, h135);
+        const double h137 = fma(x, h136, h72);
+        const double h138 = fma(y, in[35], in[61]);
+        const double h139 = fma(y, h129, h138);
+        const double h140 = fma(y, h122, h129);
+        const double h141 = fma(y, h140, h139);
+        const double h142 = fma(z, in[35], in[62]);
+        const double h143 = fma(y, h135, h142);
+        const double h144 = fma(y, h136, h143);
+        const double h145 = fma(z, in[36], in[63]);
+        const double h146 = fma(y, h132, h145);
+        const double h147 = fma(z, h136, h146);
+        const double h148 = fma(z, in[37], in[64]);
+        const double h149 = fma(z, h132, h148);
+        const double h150 = fma(z, h126, h132);
+        const double h151 = fma(z, h150, h149);
+        const double h152 = fma(x, in[30], in[51]);
+        const double h153 = fma(x, in[15], in[30]);
+        const double h154 = fma(x, h153, h152);
+        const double h155 = fma(x, in[4], in[15]);
+        const double h156 = fma(x, h155, h153);
+        const double h157 = fma(x, h156, h154);
+        const double h158 = fma(y, in[30], in[54]);
+        const double h159 = fma(y, in[15], in[33]);
+        const double h160 = fma(x, h159, h158);
+        const double h161 = fma(y, in[4], in[18]);
+        const double h162 = fma(x, h161, h159);
+        const double h163 = fma(x, h162, h160);
+        const double h164 = fma(z, in[4], in[19]);
+        const double h165 = fma(x, h164, h100);
+        const double h166 = fma(x, h165, h101);
+        const double h167 = fma(y, in[33], in[58]);
+        const double h168 = fma(y, in[18], in[37]);
+        const double h169 = fma(x, h168, h167);
+        const double h170 = fma(y, h162, h169);
+        const double h171 = fma(z, in[19], in[39]);
+        const double h172 = fma(x, h171, h112);
+        const double h173 = fma(z, h165, h172);
+        const double h174 = fma(z, in[18], in[38]);
+        const double h175 = fma(y, h164, h174);
+        const double h176 = fma(x, h175, h110);
+        const double h177 = fma(y, in[37], in[63]);
+        const double h178 = fma(y, h168, h177);
+        const double h179 = fma(y, h161, h168);
+        const double h180 = fma(y, h179, h178);
+        const double h181 = fma(y, h174, h148);
+        const double h182 = fma(y, h175, h181);
+        const double h183 = fma(z, in[38], in[65]);
+        const double h184 = fma(y, h171, h183);
+        const double h185 = fma(z, h175, h184);
+        const double h186 = fma(z, in[39], in[66]);
+        const double h187 = fma(z, h171, h186);
+        const double h188 = fma(z, h164, h171);
+        const double h189 = fma(z, h188, h187);
+        const double h190 = fma(x, in[29], in[50]);
+        const double h191 = fma(x, in[14], in[29]);
+        const double h192 = fma(x, h191, h190);
+        const double h193 = fma(x, in[5], in[14]);
+        const double h194 = fma(x, h193, h191);
+        const double h195 = fma(x, h194, h192);
+        const double h196 = fma(y, in[5], in[17]);
+        const double h197 = fma(x, h196, h97);
+        const double h198 = fma(x, h197, h98);
+        const double h199 = fma(z, in[5], in[18]);
+        const double h200 = fma(x, h199, h61);
+        const double h201 = fma(x, h200, h62);
+        const double h202 = fma(y, in[17], in[36]);
+        const double h203 = fma(x, h202, h105);
+        const double h204 = fma(y, h197, h203);
+        const double h205 = fma(x, h174, h77);
+        const double h206 = fma(z, h200, h205);
+        const double h207 = fma(y, h199, h132);
+        const double h208 = fma(x, h207, h75);
+        const double h209 = fma(y, in[36], in[62]);
+        const double h210 = fma(y, h202, h209);
+        const double h211 = fma(y, h196, h202);
+        const double h212 = fma(y, h211, h210);
+        const double h213 = fma(y, h207, h146);
+        const double h214 = fma(z, h207, h181);
+        const double h215 = fma(z, h174, h183);
+        const double h216 = fma(z, h199, h174);
+        const double h217 = fma(z, h216, h215);
+        const double h218 = fma(x, in[31], in[52]);
+        const double h219 = fma(x, in[16], in[31]);
+        const double h220 = fma(x, h219, h218);
+        const double h221 = fma(x, in[6], in[16]);
+        const double h222 = fma(x, h221, h219);
+        const double h223 = fma(x, h222, h220);
+        const double h224 = fma(y, in[6], in[20]);
+        const double h225 = fma(x, h224, h129);
+        const double h226 = fma(x, h225, h130);
+        const double h227 = fma(x, h135, h71);
+        const double h228 = fma(z, in[6], in[21]);
+        const double h229 = fma(x, h228, h135);
+        const double h230 = fma(x, h229, h227);
+        const double h231 = fma(y, in[20], in[40]);
+        const double h232 = fma(x, h231, h138);
+        const double h233 = fma(y, h225, h232);
+        const double h234 = fma(z, in[21], in[42]);
+        const double h235 = fma(x, h234, h145);
+        const double h236 = fma(z, h229, h235);
+        const double h237 = fma(z, in[20], in[41]);
+        const double h238 = fma(y, h228, h237);
+        const double h239 = fma(x, h238, h143);
+        const double h240 = fma(y, in[40], in[67]);
+        const double h241 = fma(y, h231, h240);
+        const double h242 = fma(y, h224, h231);
+        const double h243 = fma(y, h242, h241);
+        const double h244 = fma(z, in[40], in[68]);
+        const double h245 = fma(y, h237, h244);
+        const double h246 = fma(y, h238, h245);
+        const double h247 = fma(z, in[41], in[69]);
+        const double h248 = fma(y, h234, h247);
+        const double h249 = fma(z, h238, h248);
+        const double h250 = fma(z, in[42], in[70]);
+        const double h251 = fma(z, h234, h250);
+        const double h252 = fma(z, h228, h234);
+        const double h253 = fma(z, h252, h251);
+        const double h254 = fma(x, in[32], in[53]);
+        const double h255 = fma(x, in[17], in[32]);
+        const double h256 = fma(x, h255, h254);
+        const double h257 = fma(x, in[7], in[17]);
+        const double h258 = fma(x, h257, h255);
+        const double h259 = fma(x, h258, h256);
+        const double h260 = fma(y, in[7], in[21]);
+        const double h261 = fma(x, h260, h202);
+        const double h262 = fma(x, h261, h203);
+        const double h263 = fma(z, in[7], in[22]);
+        const double h264 = fma(x, h263, h132);
+        const double h265 = fma(x, h264, h133);
+        const double h266 = fma(y, in[21], in[41]);
+        const double h267 = fma(x, h266, h209);
+        const double h268 = fma(y, h261, h267);
+        const double h269 = fma(z, in[22], in[43]);
+        const double h270 = fma(x, h269, h148);
+        const double h271 = fma(z, h264, h270);
+        const double h272 = fma(y, h263, h234);
+        const double h273 = fma(x, h272, h146);
+        const double h274 = fma(y, in[41], in[68]);
+        const double h275 = fma(y, h266, h274);
+        const double h276 = fma(y, h260, h266);
+        const double h277 = fma(y, h276, h275);
+        const double h278 = fma(y, h272, h248);
+        const double h279 = fma(y, h269, h250);
+        const double h280 = fma(z, h272, h279);
+        const double h281 = fma(z, in[43], in[71]);
+        const double h282 = fma(z, h269, h281);
+        const double h283 = fma(z, h263, h269);
+        const double h284 = fma(z, h283, h282);
+        const double h285 = fma(x, in[33], in[54]);
+        const double h286 = fma(x, in[18], in[33]);
+        const double h287 = fma(x, h286, h285);
+        const double h288 = fma(x, in[8], in[18]);
+        const double h289 = fma(x, h288, h286);
+        const double h290 = fma(x, h289, h287);
+        const double h291 = fma(y, in[8], in[22]);
+        const double h292 = fma(x, h291, h168);
+        const double h293 = fma(x, h292, h169);
+        const double h294 = fma(z, in[8], in[23]);
+        const double h295 = fma(x, h294, h174);
+        const double h296 = fma(x, h295, h205);
+        const double h297 = fma(y, in[22], in[42]);
+        const double h298 = fma(x, h297, h177);
+        const double h299 = fma(y, h292, h298);
+        const double h300 = fma(z, in[23], in[44]);
+        const double h301 = fma(x, h300, h183);
+        const double h302 = fma(z, h295, h301);
+        const double h303 = fma(y, h294, h269);
+        const double h304 = fma(x, h303, h181);
+        const double h305 = fma(y, in[42], in[69]);
+        const double h306 = fma(y, h297, h305);
+        const double h307 = fma(y, h291, h297);
+        const double h308 = fma(y, h307, h306);
+        const double h309 = fma(y, h303, h279);
+        const double h310 = fma(y, h300, h281);
+        const double h311 = fma(z, h303, h310);
+        const double h312 = fma(z, in[44], in[72]);
+        const double h313 = fma(z, h300, h312);
+        const double h314 = fma(z, h294, h300);
+        const double h315 = fma(z, h314, h313);
+        const double h316 = fma(x, in[34], in[55]);
+        const double h317 = fma(x, in[19], in[34]);
+        const double h318 = fma(x, h317, h316);
+        const double h319 = fma(x, in[9], in[19]);
+        const double h320 = fma(x, h319, h317);
+        const double h321 = fma(x, h320, h318);
+        const double h322 = fma(y, in[34], in[59]);
+        const double h323 = fma(y, in[19], in[38]);
+        const double h324 = fma(x, h323, h322);
+        const double h325 = fma(y, in[9], in[23]);
+        const double h326 = fma(x, h325, h323);
+        const double h327 = fma(x, h326, h324);
+        const double h328 = fma(z, in[9], in[24]);
+        const double h329 = fma(x, h328, h171);
+        const double h330 = fma(x, h329, h172);
+        const double h331 = fma(y, in[38], in[64]);
+        const double h332 = fma(y, in[23], in[43]);
+        const double h333 = fma(x, h332, h331);
+        const double h334 = fma(y, h326, h333);
+        const double h335 = fma(z, in[24], in[45]);
+        const double h336 = fma(x, h335, h186);
+        const double h337 = fma(z, h329, h336);
+        const double h338 = fma(y, h328, h300);
+        const double h339 = fma(x, h338, h184);
+        const double h340 = fma(y, in[43], in[70]);
+        const double h341 = fma(y, h332, h340);
+        const double h342 = fma(y, h325, h332);
+        const double h343 = fma(y, h342, h341);
+        const double h344 = fma(y, h338, h310);
+        const double h345 = fma(y, h335, h312);
+        const double h346 = fma(z, h338, h345);
+        const double h347 = fma(z, in[45], in[73]);
+        const double h348 = fma(z, h335, h347);
+        const double h349 = fma(z, h328, h335);
+        const double h350 = fma(z, h349, h348);
+        out[0] = h5;
+        out[25] = h11;
+        out[50] = h17;
+        out[75] = h21;
+        out[100] = h25;
+        out[125] = h30;
+        out[150] = h34;
+        out[175] = h37;
+        out[200] = h40;
+        out[225] = h44;
+        out[250] = h50;
+        out[275] = h53;
+        out[300] = h57;
+        out[325] = h60;
+        out[350] = h63;
+        out[375] = h66;
+        out[400] = h70;
+        out[425] = h73;
+        out[450] = h76;
+        out[475] = h80;
+        out[500] = h86;
+        out[525] = h92;
+        out[550] = h95;
+        out[575] = h99;
+        out[600] = h102;
+        out[625] = h104;
+        out[650] = h108;
+        out[675] = h109;
+        out[700] = h111;
+        out[725] = h115;
+        out[750] = h121;
+        out[775] = h124;
+        out[800] = h128;
+        out[825] = h131;
+        out[850] = h134;
+        out[875] = h137;
+        out[900] = h141;
+        out[925] = h144;
+        out[950] = h147;
+        out[975] = h151;
+        out[1000] = h157;
+        out[1025] = h163;
+        out[1050] = h166;
+        out[1075] = h170;
+        out[1100] = h173;
+        out[1125] = h176;
+        out[1150] = h180;
+        out[1175] = h182;
+        out[1200] = h185;
+        out[1225] = h189;
+        out[1250] = h195;
+        out[1275] = h198;
+        out[1300] = h201;
+        out[1325] = h204;
+        out[1350] = h206;
+        out[1375] = h208;
+        out[1400] = h212;
+        out[1425] = h213;
+        out[1450] = h214;
+        out[1475] = h217;
+        out[1500] = h223;
+        out[1525] = h226;
+        out[1550] = h230;
+        out[1575] = h233;
+        out[1600] = h236;
+        out[1625] = h239;
+        out[1650] = h243;
+        out[1675] = h246;
+        out[1700] = h249;
+        out[1725] = h253;
+        out[1750] = h259;
+        out[1775] = h262;
+        out[1800] = h265;
+        out[1825] = h268;
+        out[1850] = h271;
+        out[1875] = h273;
+        out[1900] = h277;
+        out[1925] = h278;
+        out[1950] = h280;
+        out[1975] = h284;
+        out[2000] = h290;
+        out[2025] = h293;
+        out[2050] = h296;
+        out[2075] = h299;
+        out[2100] = h302;
+        out[2125] = h304;
+        out[2150] = h308;
+        out[2175] = h309;
+        out[2200] = h311;
+        out[2225] = h315;
+        out[2250] = h321;
+        out[2275] = h327;
+        out[2300] = h330;
+        out[2325] = h334;
+        out[2350] = h337;
+        out[2375] = h339;
+        out[2400] = h343;
+        out[2425] = h344;
+        out[2450] = h346;
+        out[2475] = h350;
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[0], in[10]);
+        const double h1 = fma(y, in[0], in[11]);
+        const double h2 = fma(z, in[0], in[12]);
+        const double h3 = fma(x, in[1], in[11]);
+        const double h4 = fma(y, in[1], in[13]);
+        const double h5 = fma(z, in[1], in[14]);
+        const double h6 = fma(x, in[2], in[12]);
+        const double h7 = fma(y, in[2], in[14]);
+        const double h8 = fma(z, in[2], in[15]);
+        const double h9 = fma(x, in[3], in[13]);
+        const double h10 = fma(y, in[3], in[16]);
+        const double h11 = fma(z, in[3], in[17]);
+        const double h12 = fma(x, in[4], in[15]);
+        const double h13 = fma(y, in[4], in[18]);
+        const double h14 = fma(z, in[4], in[19]);
+        const double h15 = fma(x, in[5], in[14]);
+        const double h16 = fma(y, in[5], in[17]);
+        const double h17 = fma(z, in[5], in[18]);
+        const double h18 = fma(x, in[6], in[16]);
+        const double h19 = fma(y, in[6], in[20]);
+        const double h20 = fma(z, in[6], in[21]);
+        const double h21 = fma(x, in[7], in[17]);
+        const double h22 = fma(y, in[7], in[21]);
+        const double h23 = fma(z, in[7], in[22]);
+        const double h24 = fma(x, in[8], in[18]);
+        const double h25 = fma(y, in[8], in[22]);
+        const double h26 = fma(z, in[8], in[23]);
+        const double h27 = fma(x, in[9], in[19]);
+        const double h28 = fma(y, in[9], in[23]);
+        const double h29 = fma(z, in[9], in[24]);
+        out[0] = h0 * (nrm * 0.2581988897471611);
+        out[1] = h1 * (nrm * 0.2581988897471611);
+        out[2] = h2 * (nrm * 0.2581988897471611);
+        out[3] = h3 * (nrm * 0.5773502691896258);
+        out[4] = h4 * (nrm * 0.5773502691896258);
+        out[5] = h5 * (nrm * 0.5773502691896258);
+        out[6] = h6 * (nrm * 0.5773502691896258);
+        out[7] = h7 * (nrm * 0.5773502691896258);
+        out[8] = h8 * (nrm * 0.5773502691896258);
+        out[9] = h9 * (nrm * 0.5773502691896258);
+        out[10] = h10 * (nrm * 0.5773502691896258);
+        out[11] = h11 * (nrm * 0.5773502691896258);
+        out[12] = h12 * (nrm * 0.5773502691896258);
+        out[13] = h13 * (nrm * 0.5773502691896258);
+        out[14] = h14 * (nrm * 0.5773502691896258);
+        out[15] = h15 * (nrm * 1.0);
+        out[16] = h16 * (nrm * 1.0);
+        out[17] = h17 * (nrm * 1.0);
+        out[18] = h18 * (nrm * 0.2581988897471611);
+        out[19] = h19 * (nrm * 0.2581988897471611);
+        out[20] = h20 * (nrm * 0.2581988897471611);
+        out[21] = h21 * (nrm * 0.5773502691896258);
+        out[22] = h22 * (nrm * 0.5773502691896258);
+        out[23] = h23 * (nrm * 0.5773502691896258);
+        out[24] = h24 * (nrm * 0.5773502691896258);
+        out[25] = h25 * (nrm * 0.5773502691896258);
+        out[26] = h26 * (nrm * 0.5773502691896258);
+        out[27] = h27 * (nrm * 0.2581988897471611);
+        out[28] = h28 * (nrm * 0.2581988897471611);
+        out[29] = h29 * (nrm * 0.2581988897471611);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_fffp[1850] = {
-    18, 273, 65553, 528, 131088, 65808, 783, 66063, 131343, 196623, 19, 274,
-    65554, 529, 65809, 131089, 784, 66064, 131344, 196624, 1039, 66319, 131599, 196879,
-    262159, 1293, 1548, 66828, 1803, 132363, 67083, 2058, 67338, 132618, 197898, 1294,
-    1549, 66829, 1804, 67084, 132364, 2059, 67339, 132619, 197899, 2314, 67594, 132874,
-    198154, 263434, 327693, 327948, 393228, 328203, 458763, 393483, 328458, 393738, 459018, 524298,
-    327694, 327949, 393229, 328204, 393484, 458764, 328459, 393739, 459019, 524299, 328714, 393994,
-    459274, 524554, 589834, 2568, 2823, 68103, 3078, 133638, 68358, 3333, 68613, 133893,
-    199173, 2569, 2824, 68104, 3079, 68359, 133639, 3334, 68614, 133894, 199174, 3589,
-    68869, 134149, 199429, 264709, 655368, 655623, 720903, 655878, 786438, 721158, 656133, 721413,
-    786693, 851973, 655369, 655624, 720904, 655879, 721159, 786439, 656134, 721414, 786694, 851974,
-    656389, 721669, 786949, 852229, 917509, 328968, 329223, 394503, 329478, 460038, 394758, 329733,
-    395013, 460293, 525573, 328969, 329224, 394504, 329479, 394759, 460039, 329734, 395014, 460294,
-    525574, 329989, 395269, 460549, 525829, 591109, 3843, 4098, 69378, 4353, 134913, 69633,
-    4608, 69888, 135168, 200448, 3844, 4099, 69379, 4354, 69634, 134914, 4609, 69889,
-    135169, 200449, 4864, 70144, 135424, 200704, 265984, 330243, 330498, 395778, 330753, 461313,
-    396033, 331008, 396288, 461568, 526848, 330244, 330499, 395779, 330754, 396034, 461314, 331009,
-    396289, 461569, 526849, 331264, 396544, 461824, 527104, 592384, 656643, 656898, 722178, 657153,
-    787713, 722433, 657408, 722688, 787968, 853248, 656644, 656899, 722179, 657154, 722434, 787714,
-    657409, 722689, 787969, 853249, 657664, 722944, 788224, 853504, 918784, 983043, 983298, 1048578,
-    983553, 1114113, 1048833, 983808, 1049088, 1114368, 1179648, 983044, 983299, 1048579, 983554, 1048834,
-    1114114, 983809, 1049089, 1114369, 1179649, 984064, 1049344, 1114624, 1179904, 1245184, 23, 278,
-    65558, 533, 131093, 65813, 788, 66068, 131348, 196628, 24, 279, 65559, 534,
-    65814, 131094, 789, 66069, 131349, 196629, 1044, 66324, 131604, 196884, 262164, 1298,
-    1553, 66833, 1808, 132368, 67088, 2063, 67343, 132623, 197903, 1299, 1554, 66834,
-    1809, 67089, 132369, 2064, 67344, 132624, 197904, 2319, 67599, 132879, 198159, 263439,
-    327698, 327953, 393233, 328208, 458768, 393488, 328463, 393743, 459023, 524303, 327699, 327954,
-    393234, 328209, 393489, 458769, 328464, 393744, 459024, 524304, 328719, 393999, 459279, 524559,
-    589839, 2573, 2828, 68108, 3083, 133643, 68363, 3338, 68618, 133898, 199178, 2574,
-    2829, 68109, 3084, 68364, 133644, 3339, 68619, 133899, 199179, 3594, 68874, 134154,
-    199434, 264714, 328973, 329228, 394508, 329483, 460043, 394763, 329738, 395018, 460298, 525578,
-    328974, 329229, 394509, 329484, 394764, 460044, 329739, 395019, 460299, 525579, 329994, 395274,
-    460554, 525834, 591114, 655373, 655628, 720908, 655883, 786443, 721163, 656138, 721418, 786698,
-    851978, 655374, 655629, 720909, 655884, 721164, 786444, 656139, 721419, 786699, 851979, 656394,
-    721674, 786954, 852234, 917514, 3848, 4103, 69383, 4358, 134918, 69638, 4613, 69893,
-    135173, 200453, 3849, 4104, 69384, 4359, 69639, 134919, 4614, 69894, 135174, 200454,
-    4869, 70149, 135429, 200709, 265989, 330248, 330503, 395783, 330758, 461318, 396038, 331013,
-    396293, 461573, 526853, 330249, 330504, 395784, 330759, 396039, 461319, 331014, 396294, 461574,
-    526854, 331269, 396549, 461829, 527109, 592389, 656648, 656903, 722183, 657158, 787718, 722438,
-    657413, 722693, 787973, 853253, 656649, 656904, 722184, 657159, 722439, 787719, 657414, 722694,
-    787974, 853254, 657669, 722949, 788229, 853509, 918789, 983048, 983303, 1048583, 983558, 1114118,
-    1048838, 983813, 1049093, 1114373, 1179653, 983049, 983304, 1048584, 983559, 1048839, 1114119, 983814,
-    1049094, 1114374, 1179654, 984069, 1049349, 1114629, 1179909, 1245189, 5123, 5378, 70658, 5633,
-    136193, 70913, 5888, 71168, 136448, 201728, 5124, 5379, 70659, 5634, 70914, 136194,
-    5889, 71169, 136449, 201729, 6144, 71424, 136704, 201984, 267264, 331523, 331778, 397058,
-    332033, 462593, 397313, 332288, 397568, 462848, 528128, 331524, 331779, 397059, 332034, 397314,
-    462594, 332289, 397569, 462849, 528129, 332544, 397824, 463104, 528384, 593664, 657923, 658178,
-    723458, 658433, 788993, 723713, 658688, 723968, 789248, 854528, 657924, 658179, 723459, 658434,
-    723714, 788994, 658689, 723969, 789249, 854529, 658944, 724224, 789504, 854784, 920064, 984323,
-    984578, 1049858, 984833, 1115393, 1050113, 985088, 1050368, 1115648, 1180928, 984324, 984579, 1049859,
-    984834, 1050114, 1115394, 985089, 1050369, 1115649, 1180929, 985344, 1050624, 1115904, 1181184, 1246464,
-    1310723, 1310978, 1376258, 1311233, 1441793, 1376513, 1311488, 1376768, 1442048, 1507328, 1310724, 1310979,
-    1376259, 1311234, 1376514, 1441794, 1311489, 1376769, 1442049, 1507329, 1311744, 1377024, 1442304, 1507584,
-    1572864, 28, 283, 65563, 538, 131098, 65818, 793, 66073, 131353, 196633, 29,
-    284, 65564, 539, 65819, 131099, 794, 66074, 131354, 196634, 1049, 66329, 131609,
-    196889, 262169, 1303, 1558, 66838, 1813, 132373, 67093, 2068, 67348, 132628, 197908,
-    1304, 1559, 66839, 1814, 67094, 132374, 2069, 67349, 132629, 197909, 2324, 67604,
-    132884, 198164, 263444, 327703, 327958, 393238, 328213, 458773, 393493, 328468, 393748, 459028,
-    524308, 327704, 327959, 393239, 328214, 393494, 458774, 328469, 393749, 459029, 524309, 328724,
-    394004, 459284, 524564, 589844, 2578, 2833, 68113, 3088, 133648, 68368, 3343, 68623,
-    133903, 199183, 2579, 2834, 68114, 3089, 68369, 133649, 3344, 68624, 133904, 199184,
-    3599, 68879, 134159, 199439, 264719, 328978, 329233, 394513, 329488, 460048, 394768, 329743,
-    395023, 460303, 525583, 328979, 329234, 394514, 329489, 394769, 460049, 329744, 395024, 460304,
-    525584, 329999, 395279, 460559, 525839, 591119, 655378, 655633, 720913, 655888, 786448, 721168,
-    656143, 721423, 786703, 851983, 655379, 655634, 720914, 655889, 721169, 786449, 656144, 721424,
-    786704, 851984, 656399, 721679, 786959, 852239, 917519, 3853, 4108, 69388, 4363, 134923,
-    69643, 4618, 69898, 135178, 200458, 3854, 4109, 69389, 4364, 69644, 134924, 4619,
-    69899, 135179, 200459, 4874, 70154, 135434, 200714, 265994, 330253, 330508, 395788, 330763,
-    461323, 396043, 331018, 396298, 461578, 526858, 330254, 330509, 395789, 330764, 396044, 461324,
-    331019, 396299, 461579, 526859, 331274, 396554, 461834, 527114, 592394, 656653, 656908, 722188,
-    657163, 787723, 722443, 657418, 722698, 787978, 853258, 656654, 656909, 722189, 657164, 722444,
-    787724, 657419, 722699, 787979, 853259, 657674, 722954, 788234, 853514, 918794, 983053, 983308,
-    1048588, 983563, 1114123, 1048843, 983818, 1049098, 1114378, 1179658, 983054, 983309, 1048589, 983564,
-    1048844, 1114124, 983819, 1049099, 1114379, 1179659, 984074, 1049354, 1114634, 1179914, 1245194, 5128,
-    5383, 70663, 5638, 136198, 70918, 5893, 71173, 136453, 201733, 5129, 5384, 70664,
-    5639, 70919, 136199, 5894, 71174, 136454, 201734, 6149, 71429, 136709, 201989, 267269,
-    331528, 331783, 397063, 332038, 462598, 397318, 332293, 397573, 462853, 528133, 331529, 331784,
-    397064, 332039, 397319, 462599, 332294, 397574, 462854, 528134, 332549, 397829, 463109, 528389,
-    593669, 657928, 658183, 723463, 658438, 788998, 723718, 658693, 723973, 789253, 854533, 657929,
-    658184, 723464, 658439, 723719, 788999, 658694, 723974, 789254, 854534, 658949, 724229, 789509,
-    854789, 920069, 984328, 984583, 1049863, 984838, 1115398, 1050118, 985093, 1050373, 1115653, 1180933,
-    984329, 984584, 1049864, 984839, 1050119, 1115399, 985094, 1050374, 1115654, 1180934, 985349, 1050629,
-    1115909, 1181189, 1246469, 1310728, 1310983, 1376263, 1311238, 1441798, 1376518, 1311493, 1376773, 1442053,
-    1507333, 1310729, 1310984, 1376264, 1311239, 1376519, 1441799, 1311494, 1376774, 1442054, 1507334, 1311749,
-    1377029, 1442309, 1507589, 1572869, 6403, 6658, 71938, 6913, 137473, 72193, 7168, 72448,
-    137728, 203008, 6404, 6659, 71939, 6914, 72194, 137474, 7169, 72449, 137729, 203009,
-    7424, 72704, 137984, 203264, 268544, 332803, 333058, 398338, 333313, 463873, 398593, 333568,
-    398848, 464128, 529408, 332804, 333059, 398339, 333314, 398594, 463874, 333569, 398849, 464129,
-    529409, 333824, 399104, 464384, 529664, 594944, 659203, 659458, 724738, 659713, 790273, 724993,
-    659968, 725248, 790528, 855808, 659204, 659459, 724739, 659714, 724994, 790274, 659969, 725249,
-    790529, 855809, 660224, 725504, 790784, 856064, 921344, 985603, 985858, 1051138, 986113, 1116673,
-    1051393, 986368, 1051648, 1116928, 1182208, 985604, 985859, 1051139, 986114, 1051394, 1116674, 986369,
-    1051649, 1116929, 1182209, 986624, 1051904, 1117184, 1182464, 1247744, 1312003, 1312258, 1377538, 1312513,
-    1443073, 1377793, 1312768, 1378048, 1443328, 1508608, 1312004, 1312259, 1377539, 1312514, 1377794, 1443074,
-    1312769, 1378049, 1443329, 1508609, 1313024, 1378304, 1443584, 1508864, 1574144, 1638403, 1638658, 1703938,
-    1638913, 1769473, 1704193, 1639168, 1704448, 1769728, 1835008, 1638404, 1638659, 1703939, 1638914, 1704194,
-    1769474, 1639169, 1704449, 1769729, 1835009, 1639424, 1704704, 1769984, 1835264, 1900544, 33, 288,
-    65568, 543, 131103, 65823, 798, 66078, 131358, 196638, 34, 289, 65569, 544,
-    65824, 131104, 799, 66079, 131359, 196639, 1054, 66334, 131614, 196894, 262174, 1308,
-    1563, 66843, 1818, 132378, 67098, 2073, 67353, 132633, 197913, 1309, 1564, 66844,
-    1819, 67099, 132379, 2074, 67354, 132634, 197914, 2329, 67609, 132889, 198169, 263449,
-    327708, 327963, 393243, 328218, 458778, 393498, 328473, 393753, 459033, 524313, 327709, 327964,
-    393244, 328219, 393499, 458779, 328474, 393754, 459034, 524314, 328729, 394009, 459289, 524569,
-    589849, 2583, 2838, 68118, 3093, 133653, 68373, 3348, 68628, 133908, 199188, 2584,
-    2839, 68119, 3094, 68374, 133654, 3349, 68629, 133909, 199189, 3604, 68884, 134164,
-    199444, 264724, 328983, 329238, 394518, 329493, 460053, 394773, 329748, 395028, 460308, 525588,
-    328984, 329239, 394519, 329494, 394774, 460054, 329749, 395029, 460309, 525589, 330004, 395284,
-    460564, 525844, 591124, 655383, 655638, 720918, 655893, 786453, 721173, 656148, 721428, 786708,
-    851988, 655384, 655639, 720919, 655894, 721174, 786454, 656149, 721429, 786709, 851989, 656404,
-    721684, 786964, 852244, 917524, 3858, 4113, 69393, 4368, 134928, 69648, 4623, 69903,
-    135183, 200463, 3859, 4114, 69394, 4369, 69649, 134929, 4624, 69904, 135184, 200464,
-    4879, 70159, 135439, 200719, 265999, 330258, 330513, 395793, 330768, 461328, 396048, 331023,
-    396303, 461583, 526863, 330259, 330514, 395794, 330769, 396049, 461329, 331024, 396304, 461584,
-    526864, 331279, 396559, 461839, 527119, 592399, 656658, 656913, 722193, 657168, 787728, 722448,
-    657423, 722703, 787983, 853263, 656659, 656914, 722194, 657169, 722449, 787729, 657424, 722704,
-    787984, 853264, 657679, 722959, 788239, 853519, 918799, 983058, 983313, 1048593, 983568, 1114128,
-    1048848, 983823, 1049103, 1114383, 1179663, 983059, 983314, 1048594, 983569, 1048849, 1114129, 983824,
-    1049104, 1114384, 1179664, 984079, 1049359, 1114639, 1179919, 1245199, 5133, 5388, 70668, 5643,
-    136203, 70923, 5898, 71178, 136458, 201738, 5134, 5389, 70669, 5644, 70924, 136204,
-    5899, 71179, 136459, 201739, 6154, 71434, 136714, 201994, 267274, 331533, 331788, 397068,
-    332043, 462603, 397323, 332298, 397578, 462858, 528138, 331534, 331789, 397069, 332044, 397324,
-    462604, 332299, 397579, 462859, 528139, 332554, 397834, 463114, 528394, 593674, 657933, 658188,
-    723468, 658443, 789003, 723723, 658698, 723978, 789258, 854538, 657934, 658189, 723469, 658444,
-    723724, 789004, 658699, 723979, 789259, 854539, 658954, 724234, 789514, 854794, 920074, 984333,
-    984588, 1049868, 984843, 1115403, 1050123, 985098, 1050378, 1115658, 1180938, 984334, 984589, 1049869,
-    984844, 1050124, 1115404, 985099, 1050379, 1115659, 1180939, 985354, 1050634, 1115914, 1181194, 1246474,
-    1310733, 1310988, 1376268, 1311243, 1441803, 1376523, 1311498, 1376778, 1442058, 1507338, 1310734, 1310989,
-    1376269, 1311244, 1376524, 1441804, 1311499, 1376779, 1442059, 1507339, 1311754, 1377034, 1442314, 1507594,
-    1572874, 6408, 6663, 71943, 6918, 137478, 72198, 7173, 72453, 137733, 203013, 6409,
-    6664, 71944, 6919, 72199, 137479, 7174, 72454, 137734, 203014, 7429, 72709, 137989,
-    203269, 268549, 332808, 333063, 398343, 333318, 463878, 398598, 333573, 398853, 464133, 529413,
-    332809, 333064, 398344, 333319, 398599, 463879, 333574, 398854, 464134, 529414, 333829, 399109,
-    464389, 529669, 594949, 659208, 659463, 724743, 659718, 790278, 724998, 659973, 725253, 790533,
-    855813, 659209, 659464, 724744, 659719, 724999, 790279, 659974, 725254, 790534, 855814, 660229,
-    725509, 790789, 856069, 921349, 985608, 985863, 1051143, 986118, 1116678, 1051398, 986373, 1051653,
-    1116933, 1182213, 985609, 985864, 1051144, 986119, 1051399, 1116679, 986374, 1051654, 1116934, 1182214,
-    986629, 1051909, 1117189, 1182469, 1247749, 1312008, 1312263, 1377543, 1312518, 1443078, 1377798, 1312773,
-    1378053, 1443333, 1508613, 1312009, 1312264, 1377544, 1312519, 1377799, 1443079, 1312774, 1378054, 1443334,
-    1508614, 1313029, 1378309, 1443589, 1508869, 1574149, 1638408, 1638663, 1703943, 1638918, 1769478, 1704198,
-    1639173, 1704453, 1769733, 1835013, 1638409, 1638664, 1703944, 1638919, 1704199, 1769479, 1639174, 1704454,
-    1769734, 1835014, 1639429, 1704709, 1769989, 1835269, 1900549, 7683, 7938, 73218, 8193, 138753,
-    73473, 8448, 73728, 139008, 204288, 7684, 7939, 73219, 8194, 73474, 138754, 8449,
-    73729, 139009, 204289, 8704, 73984, 139264, 204544, 269824, 334083, 334338, 399618, 334593,
-    465153, 399873, 334848, 400128, 465408, 530688, 334084, 334339, 399619, 334594, 399874, 465154,
-    334849, 400129, 465409, 530689, 335104, 400384, 465664, 530944, 596224, 660483, 660738, 726018,
-    660993, 791553, 726273, 661248, 726528, 791808, 857088, 660484, 660739, 726019, 660994, 726274,
-    791554, 661249, 726529, 791809, 857089, 661504, 726784, 792064, 857344, 922624, 986883, 987138,
-    1052418, 987393, 1117953, 1052673, 987648, 1052928, 1118208, 1183488, 986884, 987139, 1052419, 987394,
-    1052674, 1117954, 987649, 1052929, 1118209, 1183489, 987904, 1053184, 1118464, 1183744, 1249024, 1313283,
-    1313538, 1378818, 1313793, 1444353, 1379073, 1314048, 1379328, 1444608, 1509888, 1313284, 1313539, 1378819,
-    1313794, 1379074, 1444354, 1314049, 1379329, 1444609, 1509889, 1314304, 1379584, 1444864, 1510144, 1575424,
-    1639683, 1639938, 1705218, 1640193, 1770753, 1705473, 1640448, 1705728, 1771008, 1836288, 1639684, 1639939,
-    1705219, 1640194, 1705474, 1770754, 1640449, 1705729, 1771009, 1836289, 1640704, 1705984, 1771264, 1836544,
-    1901824, 1966083, 1966338, 2031618, 1966593, 2097153, 2031873, 1966848, 2032128, 2097408, 2162688, 1966084,
-    1966339, 2031619, 1966594, 2031874, 2097154, 1966849, 2032129, 2097409, 2162689, 1967104, 2032384, 2097664,
-    2162944, 2228224,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_fffp[101] = {
-    0, 4, 10, 16, 22, 28, 36, 40, 46, 52, 56, 60,
-    66, 72, 78, 84, 92, 96, 102, 108, 112, 116, 122, 128,
-    134, 140, 148, 152, 158, 164, 168, 172, 178, 184, 190, 196,
-    204, 208, 214, 220, 224, 228, 234, 240, 246, 252, 260, 264,
-    270, 276, 280, 284, 290, 296, 302, 308, 316, 320, 326, 332,
-    336, 340, 346, 352, 358, 364, 372, 376, 382, 388, 392, 396,
-    402, 408, 414, 420, 428, 432, 438, 444, 448, 452, 458, 464,
-    470, 476, 484, 488, 494, 500, 504, 508, 514, 520, 526, 532,
-    540, 544, 550, 556, 560,
-};
-__device__ const uint32_t kBraTerm_fffp[560] = {
-    68096, 197642, 196889, 65582, 68352, 66571, 132362, 131354, 66073, 65583, 68608, 66572,
-    132618, 131355, 66329, 65584, 68864, 132363, 65820, 67338, 131610, 65585, 69376, 132620,
-    65822, 67850, 131867, 65587, 69120, 66828, 67083, 65821, 67594, 66075, 66330, 65586,
-    69632, 198411, 197148, 65588, 69888, 67340, 133131, 131613, 66332, 65589, 70144, 133132,
-    66078, 67851, 131869, 65590, 70400, 198924, 197406, 65591, 68097, 197643, 196890, 65583,
-    68353, 66573, 132363, 131356, 66074, 65585, 68609, 66574, 132619, 131357, 66330, 65586,
-    68865, 132365, 65823, 67339, 131612, 65588, 69377, 132622, 65825, 67851, 131869, 65590,
-    69121, 66830, 67085, 65824, 67595, 66077, 66332, 65589, 69633, 198413, 197151, 65592,
-    69889, 67342, 133133, 131616, 66335, 65593, 70145, 133134, 66081, 67853, 131872, 65594,
-    70401, 198926, 197409, 65595, 68098, 197644, 196891, 65584, 68354, 66574, 132364, 131357,
-    66075, 65586, 68610, 66575, 132620, 131358, 66331, 65587, 68866, 132366, 65824, 67340,
-    131613, 65589, 69378, 132623, 65826, 67852, 131870, 65591, 69122, 66831, 67086, 65825,
-    67596, 66078, 66333, 65590, 69634, 198414, 197152, 65593, 69890, 67343, 133134, 131617,
-    66336, 65594, 70146, 133135, 66082, 67854, 131873, 65595, 70402, 198927, 197410, 65596,
-    68099, 197645, 196892, 65585, 68355, 66576, 132365, 131359, 66076, 65588, 68611, 66577,
-    132621, 131360, 66332, 65589, 68867, 132368, 65827, 67341, 131615, 65592, 69379, 132625,
-    65829, 67853, 131872, 65594, 69123, 66833, 67088, 65828, 67597, 66080, 66335, 65593,
-    69635, 198416, 197155, 65597, 69891, 67345, 133136, 131620, 66339, 65598, 70147, 133137,
-    66085, 67856, 131876, 65599, 70403, 198929, 197413, 65600, 68100, 197647, 196894, 65587,
-    68356, 66578, 132367, 131361, 66078, 65590, 68612, 66579, 132623, 131362, 66334, 65591,
-    68868, 132370, 65829, 67343, 131617, 65594, 69380, 132627, 65831, 67855, 131874, 65596,
-    69124, 66835, 67090, 65830, 67599, 66082, 66337, 65595, 69636, 198418, 197157, 65599,
-    69892, 67347, 133138, 131622, 66341, 65600, 70148, 133139, 66087, 67858, 131878, 65601,
-    70404, 198931, 197415, 65602, 68101, 197646, 196893, 65586, 68357, 66577, 132366, 131360,
-    66077, 65589, 68613, 66578, 132622, 131361, 66333, 65590, 68869, 132369, 65828, 67342,
-    131616, 65593, 69381, 132626, 65830, 67854, 131873, 65595, 69125, 66834, 67089, 65829,
-    67598, 66081, 66336, 65594, 69637, 198417, 197156, 65598, 69893, 67346, 133137, 131621,
-    66340, 65599, 70149, 133138, 66086, 67857, 131877, 65600, 70405, 198930, 197414, 65601,
-    68102, 197648, 196895, 65588, 68358, 66580, 132368, 131363, 66079, 65592, 68614, 66581,
-    132624, 131364, 66335, 65593, 68870, 132372, 65832, 67344, 131619, 65597, 69382, 132629,
-    65834, 67856, 131876, 65599, 69126, 66837, 67092, 65833, 67600, 66084, 66339, 65598,
-    69638, 198420, 197160, 65603, 69894, 67349, 133140, 131625, 66344, 65604, 70150, 133141,
-    66090, 67860, 131881, 65605, 70406, 198933, 197418, 65606, 68103, 197649, 196896, 65589,
-    68359, 66581, 132369, 131364, 66080, 65593, 68615, 66582, 132625, 131365, 66336, 65594,
-    68871, 132373, 65833, 67345, 131620, 65598, 69383, 132630, 65835, 67857, 131877, 65600,
-    69127, 66838, 67093, 65834, 67601, 66085, 66340, 65599, 69639, 198421, 197161, 65604,
-    69895, 67350, 133141, 131626, 66345, 65605, 70151, 133142, 66091, 67861, 131882, 65606,
-    70407, 198934, 197419, 65607, 68104, 197650, 196897, 65590, 68360, 66582, 132370, 131365,
-    66081, 65594, 68616, 66583, 132626, 131366, 66337, 65595, 68872, 132374, 65834, 67346,
-    131621, 65599, 69384, 132631, 65836, 67858, 131878, 65601, 69128, 66839, 67094, 65835,
-    67602, 66086, 66341, 65600, 69640, 198422, 197162, 65605, 69896, 67351, 133142, 131627,
-    66346, 65606, 70152, 133143, 66092, 67862, 131883, 65607, 70408, 198935, 197420, 65608,
-    68105, 197651, 196898, 65591, 68361, 66583, 132371, 131366, 66082, 65595, 68617, 66584,
-    132627, 131367, 66338, 65596, 68873, 132375, 65835, 67347, 131622, 65600, 69385, 132632,
-    65837, 67859, 131879, 65602, 69129, 66840, 67095, 65836, 67603, 66087, 66342, 65601,
-    69641, 198423, 197163, 65606, 69897, 67352, 133143, 131628, 66347, 65607, 70153, 133144,
-    66093, 67863, 131884, 65608, 70409, 198936, 197421, 65609,
-};
-__device__ const uint16_t kKetOff_fffp[31] = {
-    0, 2, 4, 6, 8, 10, 12, 14, 16, 18, 20, 22,
-    24, 26, 28, 30, 32, 34, 36, 38, 40, 42, 44, 46,
-    48, 50, 52, 54, 56, 58, 60,
-};
-__device__ const uint32_t kKetTerm_fffp[60] = {
-    65792, 65546, 66048, 65547, 66304, 65548, 65793, 65547, 66049, 65549, 66305, 65550,
-    65794, 65548, 66050, 65550, 66306, 65551, 65795, 65549, 66051, 65552, 66307, 65553,
-    65796, 65551, 66052, 65554, 66308, 65555, 65797, 65550, 66053, 65553, 66309, 65554,
-    65798, 65552, 66054, 65556, 66310, 65557, 65799, 65553, 66055, 65557, 66311, 65558,
-    65800, 65554, 66056, 65558, 66312, 65559, 65801, 65555, 66057, 65559, 66313, 65560,
-};
 __device__ const double kNormAB_fffp[100] = {
     0.06666666666666665, 0.14907119849998599, 0.14907119849998599, 0.14907119849998599,
     0.14907119849998599, 0.2581988897471611, 0.06666666666666665, 0.14907119849998599,
@@ -277,21 +639,12 @@ __device__ const double kNormAB_fffp[100] = {
     0.14907119849998599, 0.14907119849998599, 0.14907119849998599, 0.2581988897471611,
     0.06666666666666665, 0.14907119849998599, 0.14907119849998599, 0.06666666666666665,
 };
-__device__ const double kNormCD_fffp[30] = {
-    0.2581988897471611, 0.2581988897471611, 0.2581988897471611, 0.5773502691896258,
-    0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
-    0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
-    0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 1.0,
-    1.0, 1.0, 0.2581988897471611, 0.2581988897471611,
-    0.2581988897471611, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
-    0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.2581988897471611,
-    0.2581988897471611, 0.2581988897471611,
-};
 
+// column components cx | cy << 4 | cz << 8
+__device__ const uint16_t kCol_fffp[25] = { 3, 18, 258, 33, 513, 273, 48, 288, 528, 768, 4, 19, 259, 34, 274, 514, 49, 289, 529, 769, 64, 304, 544, 784, 1024 };
 
 __device__ __forceinline__ RysClassTabs tabs_fffp() {
-    return RysClassTabs{kBlk_fffp, kBraOff_fffp, kBraTerm_fffp, kKetOff_fffp, kKetTerm_fffp,
-                        kNormAB_fffp, kNormCD_fffp, nullptr};
+    return RysClassTabs{kNormAB_fffp, kCol_fffp};
 }
 
 template <int MIXED>
@@ -304,8 +657,8 @@ static void rys_prepare_fffp() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_fffp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 45680);
-        cudaFuncSetAttribute(rys_queue_fffp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 45680);
+        cudaFuncSetAttribute(rys_queue_fffp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 179200);
+        cudaFuncSetAttribute(rys_queue_fffp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 179200);
 
         done[dev] = true;
     }
@@ -317,16 +670,16 @@ void launch_rys_fffp(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_fffp();
     constexpr int ng = 128 / C_fffp::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_fffp<1><<<grid, 128, 45680, s>>>(Q, R);
-    else rys_queue_fffp<0><<<grid, 128, 45680, s>>>(Q, R);
+    if (mixed) rys_queue_fffp<1><<<grid, 128, 179200, s>>>(Q, R);
+    else rys_queue_fffp<0><<<grid, 128, 179200, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_fffp(int mixed) {
     rys_prepare_fffp();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fffp<1>, 128, 45680);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fffp<0>, 128, 45680);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fffp<1>, 128, 179200);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fffp<0>, 128, 179200);
     return n;
 }
 

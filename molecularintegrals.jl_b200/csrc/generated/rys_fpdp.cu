@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (fp|dp).  Do not edit.
-// roots 4, block 25 x 16, outputs 30 x 18, group 32 threads,
-// 8 primitive quartets per batch, 1 slot(s), 1 accumulators per thread, 62720 B shared per block, column mode.
+// roots 4, block 25 x 16, outputs 30 x 18, group 32 threads, 2 ket pairs a round,
+// 4 primitive quartets per ket pair and batch, 69120 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,11 +11,10 @@ struct C_fpdp {
     static constexpr int NA = 25, NC = 16, NBLK = 400;
     static constexpr int NB = 3, ND = 3;
     static constexpr int NAB = 30, NCD = 18;
-    static constexpr int G = 32, NPB = 8, NSLOT = 1, ACC = 1;
-    static constexpr int S = 20;
-    static constexpr int SMEM_GROUP = 1960;
-    static constexpr bool COL = true;
-    // stage 2, column mode: acc[row] += x[ax] y[ay] z[az] for the column's table columns
+    static constexpr int G = 32, W = 2, H = 1, PB = 4;
+    static constexpr int S = 20, SI = 61, NCP = 17, NCDP = 19;
+    static constexpr int SMEM_GROUP = 2160;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
     __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
         acc[0] = fma(x[3] * y[0], z[0], acc[0]);
@@ -44,68 +43,111 @@ struct C_fpdp {
         acc[23] = fma(x[0] * y[1], z[3], acc[23]);
         acc[24] = fma(x[0] * y[0], z[4], acc[24]);
     }
-    static constexpr int NCOLS = 16;
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[0], in[10]);
+        const double h1 = fma(y, in[0], in[11]);
+        const double h2 = fma(z, in[0], in[12]);
+        const double h3 = fma(x, in[1], in[11]);
+        const double h4 = fma(y, in[1], in[13]);
+        const double h5 = fma(z, in[1], in[14]);
+        const double h6 = fma(x, in[2], in[12]);
+        const double h7 = fma(y, in[2], in[14]);
+        const double h8 = fma(z, in[2], in[15]);
+        const double h9 = fma(x, in[3], in[13]);
+        const double h10 = fma(y, in[3], in[16]);
+        const double h11 = fma(z, in[3], in[17]);
+        const double h12 = fma(x, in[4], in[15]);
+        const double h13 = fma(y, in[4], in[18]);
+        const double h14 = fma(z, in[4], in[19]);
+        const double h15 = fma(x, in[5], in[14]);
+        const double h16 = fma(y, in[5], in[17]);
+        const double h17 = fma(z, in[5], in[18]);
+        const double h18 = fma(x, in[6], in[16]);
+        const double h19 = fma(y, in[6], in[20]);
+        const double h20 = fma(z, in[6], in[21]);
+        const double h21 = fma(x, in[7], in[17]);
+        const double h22 = fma(y, in[7], in[21]);
+        const double h23 = fma(z, in[7], in[22]);
+        const double h24 = fma(x, in[8], in[18]);
+        const double h25 = fma(y, in[8], in[22]);
+        const double h26 = fma(z, in[8], in[23]);
+        const double h27 = fma(x, in[9], in[19]);
+        const double h28 = fma(y, in[9], in[23]);
+        const double h29 = fma(z, in[9], in[24]);
+        out[0] = h0;
+        out[17] = h1;
+        out[34] = h2;
+        out[51] = h3;
+        out[68] = h4;
+        out[85] = h5;
+        out[102] = h6;
+        out[119] = h7;
+        out[136] = h8;
+        out[153] = h9;
+        out[170] = h10;
+        out[187] = h11;
+        out[204] = h12;
+        out[221] = h13;
+        out[238] = h14;
+        out[255] = h15;
+        out[272] = h16;
+        out[289] = h17;
+        out[306] = h18;
+        out[323] = h19;
+        out[340] = h20;
+        out[357] = h21;
+        out[374] = h22;
+        out[391] = h23;
+        out[408] = h24;
+        out[425] = h25;
+        out[442] = h26;
+        out[459] = h27;
+        out[476] = h28;
+        out[493] = h29;
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[0], in[6]);
+        const double h1 = fma(y, in[0], in[7]);
+        const double h2 = fma(z, in[0], in[8]);
+        const double h3 = fma(x, in[1], in[7]);
+        const double h4 = fma(y, in[1], in[9]);
+        const double h5 = fma(z, in[1], in[11]);
+        const double h6 = fma(x, in[2], in[8]);
+        const double h7 = fma(y, in[2], in[11]);
+        const double h8 = fma(z, in[2], in[10]);
+        const double h9 = fma(x, in[3], in[9]);
+        const double h10 = fma(y, in[3], in[12]);
+        const double h11 = fma(z, in[3], in[13]);
+        const double h12 = fma(x, in[4], in[11]);
+        const double h13 = fma(y, in[4], in[13]);
+        const double h14 = fma(z, in[4], in[14]);
+        const double h15 = fma(x, in[5], in[10]);
+        const double h16 = fma(y, in[5], in[14]);
+        const double h17 = fma(z, in[5], in[15]);
+        out[0] = h0 * (nrm * 0.5773502691896258);
+        out[1] = h1 * (nrm * 0.5773502691896258);
+        out[2] = h2 * (nrm * 0.5773502691896258);
+        out[3] = h3 * (nrm * 1.0);
+        out[4] = h4 * (nrm * 1.0);
+        out[5] = h5 * (nrm * 1.0);
+        out[6] = h6 * (nrm * 1.0);
+        out[7] = h7 * (nrm * 1.0);
+        out[8] = h8 * (nrm * 1.0);
+        out[9] = h9 * (nrm * 0.5773502691896258);
+        out[10] = h10 * (nrm * 0.5773502691896258);
+        out[11] = h11 * (nrm * 0.5773502691896258);
+        out[12] = h12 * (nrm * 1.0);
+        out[13] = h13 * (nrm * 1.0);
+        out[14] = h14 * (nrm * 1.0);
+        out[15] = h15 * (nrm * 0.5773502691896258);
+        out[16] = h16 * (nrm * 0.5773502691896258);
+        out[17] = h17 * (nrm * 0.5773502691896258);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_fpdp[400] = {
-    14, 269, 65549, 524, 65804, 131084, 15, 270, 65550, 525, 131085, 65805,
-    780, 66060, 131340, 196620, 1034, 1289, 66569, 1544, 66824, 132104, 1035, 1290,
-    66570, 1545, 132105, 66825, 1800, 67080, 132360, 197640, 262154, 262409, 327689, 262664,
-    327944, 393224, 262155, 262410, 327690, 262665, 393225, 327945, 262920, 328200, 393480, 458760,
-    2054, 2309, 67589, 2564, 67844, 133124, 2055, 2310, 67590, 2565, 133125, 67845,
-    2820, 68100, 133380, 198660, 524294, 524549, 589829, 524804, 590084, 655364, 524295, 524550,
-    589830, 524805, 655365, 590085, 525060, 590340, 655620, 720900, 263174, 263429, 328709, 263684,
-    328964, 394244, 263175, 263430, 328710, 263685, 394245, 328965, 263940, 329220, 394500, 459780,
-    3074, 3329, 68609, 3584, 68864, 134144, 3075, 3330, 68610, 3585, 134145, 68865,
-    3840, 69120, 134400, 199680, 264194, 264449, 329729, 264704, 329984, 395264, 264195, 264450,
-    329730, 264705, 395265, 329985, 264960, 330240, 395520, 460800, 525314, 525569, 590849, 525824,
-    591104, 656384, 525315, 525570, 590850, 525825, 656385, 591105, 526080, 591360, 656640, 721920,
-    786434, 786689, 851969, 786944, 852224, 917504, 786435, 786690, 851970, 786945, 917505, 852225,
-    787200, 852480, 917760, 983040, 18, 273, 65553, 528, 65808, 131088, 19, 274,
-    65554, 529, 131089, 65809, 784, 66064, 131344, 196624, 1038, 1293, 66573, 1548,
-    66828, 132108, 1039, 1294, 66574, 1549, 132109, 66829, 1804, 67084, 132364, 197644,
-    262158, 262413, 327693, 262668, 327948, 393228, 262159, 262414, 327694, 262669, 393229, 327949,
-    262924, 328204, 393484, 458764, 2058, 2313, 67593, 2568, 67848, 133128, 2059, 2314,
-    67594, 2569, 133129, 67849, 2824, 68104, 133384, 198664, 263178, 263433, 328713, 263688,
-    328968, 394248, 263179, 263434, 328714, 263689, 394249, 328969, 263944, 329224, 394504, 459784,
-    524298, 524553, 589833, 524808, 590088, 655368, 524299, 524554, 589834, 524809, 655369, 590089,
-    525064, 590344, 655624, 720904, 3078, 3333, 68613, 3588, 68868, 134148, 3079, 3334,
-    68614, 3589, 134149, 68869, 3844, 69124, 134404, 199684, 264198, 264453, 329733, 264708,
-    329988, 395268, 264199, 264454, 329734, 264709, 395269, 329989, 264964, 330244, 395524, 460804,
-    525318, 525573, 590853, 525828, 591108, 656388, 525319, 525574, 590854, 525829, 656389, 591109,
-    526084, 591364, 656644, 721924, 786438, 786693, 851973, 786948, 852228, 917508, 786439, 786694,
-    851974, 786949, 917509, 852229, 787204, 852484, 917764, 983044, 4098, 4353, 69633, 4608,
-    69888, 135168, 4099, 4354, 69634, 4609, 135169, 69889, 4864, 70144, 135424, 200704,
-    265218, 265473, 330753, 265728, 331008, 396288, 265219, 265474, 330754, 265729, 396289, 331009,
-    265984, 331264, 396544, 461824, 526338, 526593, 591873, 526848, 592128, 657408, 526339, 526594,
-    591874, 526849, 657409, 592129, 527104, 592384, 657664, 722944, 787458, 787713, 852993, 787968,
-    853248, 918528, 787459, 787714, 852994, 787969, 918529, 853249, 788224, 853504, 918784, 984064,
-    1048578, 1048833, 1114113, 1049088, 1114368, 1179648, 1048579, 1048834, 1114114, 1049089, 1179649, 1114369,
-    1049344, 1114624, 1179904, 1245184,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_fpdp[31] = {
-    0, 2, 4, 6, 8, 10, 12, 14, 16, 18, 20, 22,
-    24, 26, 28, 30, 32, 34, 36, 38, 40, 42, 44, 46,
-    48, 50, 52, 54, 56, 58, 60,
-};
-__device__ const uint32_t kBraTerm_fpdp[60] = {
-    65792, 65546, 66048, 65547, 66304, 65548, 65793, 65547, 66049, 65549, 66305, 65550,
-    65794, 65548, 66050, 65550, 66306, 65551, 65795, 65549, 66051, 65552, 66307, 65553,
-    65796, 65551, 66052, 65554, 66308, 65555, 65797, 65550, 66053, 65553, 66309, 65554,
-    65798, 65552, 66054, 65556, 66310, 65557, 65799, 65553, 66055, 65557, 66311, 65558,
-    65800, 65554, 66056, 65558, 66312, 65559, 65801, 65555, 66057, 65559, 66313, 65560,
-};
-__device__ const uint16_t kKetOff_fpdp[19] = {
-    0, 2, 4, 6, 8, 10, 12, 14, 16, 18, 20, 22,
-    24, 26, 28, 30, 32, 34, 36,
-};
-__device__ const uint32_t kKetTerm_fpdp[36] = {
-    65792, 65542, 66048, 65543, 66304, 65544, 65793, 65543, 66049, 65545, 66305, 65547,
-    65794, 65544, 66050, 65547, 66306, 65546, 65795, 65545, 66051, 65548, 66307, 65549,
-    65796, 65547, 66052, 65549, 66308, 65550, 65797, 65546, 66053, 65550, 66309, 65551,
-};
 __device__ const double kNormAB_fpdp[30] = {
     0.2581988897471611, 0.2581988897471611, 0.2581988897471611, 0.5773502691896258,
     0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
@@ -116,21 +158,12 @@ __device__ const double kNormAB_fpdp[30] = {
     0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.2581988897471611,
     0.2581988897471611, 0.2581988897471611,
 };
-__device__ const double kNormCD_fpdp[18] = {
-    0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 1.0,
-    1.0, 1.0, 1.0, 1.0,
-    1.0, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
-    1.0, 1.0, 1.0, 0.5773502691896258,
-    0.5773502691896258, 0.5773502691896258,
-};
-
 
 // column components cx | cy << 4 | cz << 8
 __device__ const uint16_t kCol_fpdp[16] = { 2, 17, 257, 32, 272, 512, 3, 18, 258, 33, 513, 273, 48, 288, 528, 768 };
 
 __device__ __forceinline__ RysClassTabs tabs_fpdp() {
-    return RysClassTabs{kBlk_fpdp, kBraOff_fpdp, kBraTerm_fpdp, kKetOff_fpdp, kKetTerm_fpdp,
-                        kNormAB_fpdp, kNormCD_fpdp, kCol_fpdp};
+    return RysClassTabs{kNormAB_fpdp, kCol_fpdp};
 }
 
 template <int MIXED>
@@ -143,8 +176,8 @@ static void rys_prepare_fpdp() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_fpdp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 62720);
-        cudaFuncSetAttribute(rys_queue_fpdp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 62720);
+        cudaFuncSetAttribute(rys_queue_fpdp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 69120);
+        cudaFuncSetAttribute(rys_queue_fpdp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 69120);
 
         done[dev] = true;
     }
@@ -156,16 +189,16 @@ void launch_rys_fpdp(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_fpdp();
     constexpr int ng = 128 / C_fpdp::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_fpdp<1><<<grid, 128, 62720, s>>>(Q, R);
-    else rys_queue_fpdp<0><<<grid, 128, 62720, s>>>(Q, R);
+    if (mixed) rys_queue_fpdp<1><<<grid, 128, 69120, s>>>(Q, R);
+    else rys_queue_fpdp<0><<<grid, 128, 69120, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_fpdp(int mixed) {
     rys_prepare_fpdp();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fpdp<1>, 128, 62720);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fpdp<0>, 128, 62720);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fpdp<1>, 128, 69120);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fpdp<0>, 128, 69120);
     return n;
 }
 

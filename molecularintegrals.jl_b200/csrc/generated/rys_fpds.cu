@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (fp|ds).  Do not edit.
-// roots 4, block 25 x 6, outputs 30 x 6, group 64 threads,
-// 16 primitive quartets per batch, 1 slot(s), 3 accumulators per thread, 46720 B shared per block.
+// roots 4, block 25 x 6, outputs 30 x 6, group 32 threads, 5 ket pairs a round,
+// 1 primitive quartets per ket pair and batch, 67200 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,49 +11,113 @@ struct C_fpds {
     static constexpr int NA = 25, NC = 6, NBLK = 150;
     static constexpr int NB = 3, ND = 1;
     static constexpr int NAB = 30, NCD = 6;
-    static constexpr int G = 64, NPB = 16, NSLOT = 1, ACC = 3;
-    static constexpr int S = 15;
-    static constexpr int SMEM_GROUP = 2920;
-    static constexpr bool COL = false;
+    static constexpr int G = 32, W = 5, H = 1, PB = 1;
+    static constexpr int S = 15, SI = 45, NCP = 7, NCDP = 7;
+    static constexpr int SMEM_GROUP = 2100;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
-    __device__ __forceinline__ static void col_update(const T *, const T *, const T *, A *) {}
+    __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
+        acc[0] = fma(x[3] * y[0], z[0], acc[0]);
+        acc[1] = fma(x[2] * y[1], z[0], acc[1]);
+        acc[2] = fma(x[2] * y[0], z[1], acc[2]);
+        acc[3] = fma(x[1] * y[2], z[0], acc[3]);
+        acc[4] = fma(x[1] * y[0], z[2], acc[4]);
+        acc[5] = fma(x[1] * y[1], z[1], acc[5]);
+        acc[6] = fma(x[0] * y[3], z[0], acc[6]);
+        acc[7] = fma(x[0] * y[2], z[1], acc[7]);
+        acc[8] = fma(x[0] * y[1], z[2], acc[8]);
+        acc[9] = fma(x[0] * y[0], z[3], acc[9]);
+        acc[10] = fma(x[4] * y[0], z[0], acc[10]);
+        acc[11] = fma(x[3] * y[1], z[0], acc[11]);
+        acc[12] = fma(x[3] * y[0], z[1], acc[12]);
+        acc[13] = fma(x[2] * y[2], z[0], acc[13]);
+        acc[14] = fma(x[2] * y[1], z[1], acc[14]);
+        acc[15] = fma(x[2] * y[0], z[2], acc[15]);
+        acc[16] = fma(x[1] * y[3], z[0], acc[16]);
+        acc[17] = fma(x[1] * y[2], z[1], acc[17]);
+        acc[18] = fma(x[1] * y[1], z[2], acc[18]);
+        acc[19] = fma(x[1] * y[0], z[3], acc[19]);
+        acc[20] = fma(x[0] * y[4], z[0], acc[20]);
+        acc[21] = fma(x[0] * y[3], z[1], acc[21]);
+        acc[22] = fma(x[0] * y[2], z[2], acc[22]);
+        acc[23] = fma(x[0] * y[1], z[3], acc[23]);
+        acc[24] = fma(x[0] * y[0], z[4], acc[24]);
+    }
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[0], in[10]);
+        const double h1 = fma(y, in[0], in[11]);
+        const double h2 = fma(z, in[0], in[12]);
+        const double h3 = fma(x, in[1], in[11]);
+        const double h4 = fma(y, in[1], in[13]);
+        const double h5 = fma(z, in[1], in[14]);
+        const double h6 = fma(x, in[2], in[12]);
+        const double h7 = fma(y, in[2], in[14]);
+        const double h8 = fma(z, in[2], in[15]);
+        const double h9 = fma(x, in[3], in[13]);
+        const double h10 = fma(y, in[3], in[16]);
+        const double h11 = fma(z, in[3], in[17]);
+        const double h12 = fma(x, in[4], in[15]);
+        const double h13 = fma(y, in[4], in[18]);
+        const double h14 = fma(z, in[4], in[19]);
+        const double h15 = fma(x, in[5], in[14]);
+        const double h16 = fma(y, in[5], in[17]);
+        const double h17 = fma(z, in[5], in[18]);
+        const double h18 = fma(x, in[6], in[16]);
+        const double h19 = fma(y, in[6], in[20]);
+        const double h20 = fma(z, in[6], in[21]);
+        const double h21 = fma(x, in[7], in[17]);
+        const double h22 = fma(y, in[7], in[21]);
+        const double h23 = fma(z, in[7], in[22]);
+        const double h24 = fma(x, in[8], in[18]);
+        const double h25 = fma(y, in[8], in[22]);
+        const double h26 = fma(z, in[8], in[23]);
+        const double h27 = fma(x, in[9], in[19]);
+        const double h28 = fma(y, in[9], in[23]);
+        const double h29 = fma(z, in[9], in[24]);
+        out[0] = h0;
+        out[7] = h1;
+        out[14] = h2;
+        out[21] = h3;
+        out[28] = h4;
+        out[35] = h5;
+        out[42] = h6;
+        out[49] = h7;
+        out[56] = h8;
+        out[63] = h9;
+        out[70] = h10;
+        out[77] = h11;
+        out[84] = h12;
+        out[91] = h13;
+        out[98] = h14;
+        out[105] = h15;
+        out[112] = h16;
+        out[119] = h17;
+        out[126] = h18;
+        out[133] = h19;
+        out[140] = h20;
+        out[147] = h21;
+        out[154] = h22;
+        out[161] = h23;
+        out[168] = h24;
+        out[175] = h25;
+        out[182] = h26;
+        out[189] = h27;
+        out[196] = h28;
+        out[203] = h29;
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        out[0] = in[0] * (nrm * 0.5773502691896258);
+        out[1] = in[1] * (nrm * 1.0);
+        out[2] = in[2] * (nrm * 1.0);
+        out[3] = in[3] * (nrm * 0.5773502691896258);
+        out[4] = in[4] * (nrm * 1.0);
+        out[5] = in[5] * (nrm * 0.5773502691896258);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_fpds[150] = {
-    11, 266, 65546, 521, 65801, 131081, 776, 1031, 66311, 1286, 66566, 131846,
-    196616, 196871, 262151, 197126, 262406, 327686, 1541, 1796, 67076, 2051, 67331, 132611,
-    393221, 393476, 458756, 393731, 459011, 524291, 197381, 197636, 262916, 197891, 263171, 328451,
-    2306, 2561, 67841, 2816, 68096, 133376, 198146, 198401, 263681, 198656, 263936, 329216,
-    393986, 394241, 459521, 394496, 459776, 525056, 589826, 590081, 655361, 590336, 655616, 720896,
-    14, 269, 65549, 524, 65804, 131084, 779, 1034, 66314, 1289, 66569, 131849,
-    196619, 196874, 262154, 197129, 262409, 327689, 1544, 1799, 67079, 2054, 67334, 132614,
-    197384, 197639, 262919, 197894, 263174, 328454, 393224, 393479, 458759, 393734, 459014, 524294,
-    2309, 2564, 67844, 2819, 68099, 133379, 198149, 198404, 263684, 198659, 263939, 329219,
-    393989, 394244, 459524, 394499, 459779, 525059, 589829, 590084, 655364, 590339, 655619, 720899,
-    3074, 3329, 68609, 3584, 68864, 134144, 198914, 199169, 264449, 199424, 264704, 329984,
-    394754, 395009, 460289, 395264, 460544, 525824, 590594, 590849, 656129, 591104, 656384, 721664,
-    786434, 786689, 851969, 786944, 852224, 917504,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_fpds[31] = {
-    0, 2, 4, 6, 8, 10, 12, 14, 16, 18, 20, 22,
-    24, 26, 28, 30, 32, 34, 36, 38, 40, 42, 44, 46,
-    48, 50, 52, 54, 56, 58, 60,
-};
-__device__ const uint32_t kBraTerm_fpds[60] = {
-    65792, 65546, 66048, 65547, 66304, 65548, 65793, 65547, 66049, 65549, 66305, 65550,
-    65794, 65548, 66050, 65550, 66306, 65551, 65795, 65549, 66051, 65552, 66307, 65553,
-    65796, 65551, 66052, 65554, 66308, 65555, 65797, 65550, 66053, 65553, 66309, 65554,
-    65798, 65552, 66054, 65556, 66310, 65557, 65799, 65553, 66055, 65557, 66311, 65558,
-    65800, 65554, 66056, 65558, 66312, 65559, 65801, 65555, 66057, 65559, 66313, 65560,
-};
-__device__ const uint16_t kKetOff_fpds[7] = {
-    0, 1, 2, 3, 4, 5, 6,
-};
-__device__ const uint32_t kKetTerm_fpds[6] = {
-    65536, 65537, 65538, 65539, 65540, 65541,
-};
 __device__ const double kNormAB_fpds[30] = {
     0.2581988897471611, 0.2581988897471611, 0.2581988897471611, 0.5773502691896258,
     0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
@@ -64,15 +128,12 @@ __device__ const double kNormAB_fpds[30] = {
     0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.2581988897471611,
     0.2581988897471611, 0.2581988897471611,
 };
-__device__ const double kNormCD_fpds[6] = {
-    0.5773502691896258, 1.0, 1.0, 0.5773502691896258,
-    1.0, 0.5773502691896258,
-};
 
+// column components cx | cy << 4 | cz << 8
+__device__ const uint16_t kCol_fpds[6] = { 2, 17, 257, 32, 272, 512 };
 
 __device__ __forceinline__ RysClassTabs tabs_fpds() {
-    return RysClassTabs{kBlk_fpds, kBraOff_fpds, kBraTerm_fpds, kKetOff_fpds, kKetTerm_fpds,
-                        kNormAB_fpds, kNormCD_fpds, nullptr};
+    return RysClassTabs{kNormAB_fpds, kCol_fpds};
 }
 
 template <int MIXED>
@@ -85,8 +146,8 @@ static void rys_prepare_fpds() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_fpds<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 46720);
-        cudaFuncSetAttribute(rys_queue_fpds<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 46720);
+        cudaFuncSetAttribute(rys_queue_fpds<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 67200);
+        cudaFuncSetAttribute(rys_queue_fpds<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 67200);
 
         done[dev] = true;
     }
@@ -98,16 +159,16 @@ void launch_rys_fpds(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_fpds();
     constexpr int ng = 128 / C_fpds::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_fpds<1><<<grid, 128, 46720, s>>>(Q, R);
-    else rys_queue_fpds<0><<<grid, 128, 46720, s>>>(Q, R);
+    if (mixed) rys_queue_fpds<1><<<grid, 128, 67200, s>>>(Q, R);
+    else rys_queue_fpds<0><<<grid, 128, 67200, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_fpds(int mixed) {
     rys_prepare_fpds();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fpds<1>, 128, 46720);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fpds<0>, 128, 46720);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fpds<1>, 128, 67200);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fpds<0>, 128, 67200);
     return n;
 }
 

@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (fp|fp).  Do not edit.
-// roots 5, block 25 x 25, outputs 30 x 30, group 32 threads,
-// 6 primitive quartets per batch, 1 slot(s), 1 accumulators per thread, 73280 B shared per block, column mode.
+// roots 5, block 25 x 25, outputs 30 x 30, group 32 threads, 1 ket pairs a round,
+// 4 primitive quartets per ket pair and batch, 53760 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,11 +11,10 @@ struct C_fpfp {
     static constexpr int NA = 25, NC = 25, NBLK = 625;
     static constexpr int NB = 3, ND = 3;
     static constexpr int NAB = 30, NCD = 30;
-    static constexpr int G = 32, NPB = 6, NSLOT = 1, ACC = 1;
-    static constexpr int S = 25;
-    static constexpr int SMEM_GROUP = 2290;
-    static constexpr bool COL = true;
-    // stage 2, column mode: acc[row] += x[ax] y[ay] z[az] for the column's table columns
+    static constexpr int G = 32, W = 1, H = 1, PB = 4;
+    static constexpr int S = 25, SI = 75, NCP = 25, NCDP = 31;
+    static constexpr int SMEM_GROUP = 1680;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
     __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
         acc[0] = fma(x[3] * y[0], z[0], acc[0]);
@@ -44,90 +43,135 @@ struct C_fpfp {
         acc[23] = fma(x[0] * y[1], z[3], acc[23]);
         acc[24] = fma(x[0] * y[0], z[4], acc[24]);
     }
-    static constexpr int NCOLS = 25;
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[0], in[10]);
+        const double h1 = fma(y, in[0], in[11]);
+        const double h2 = fma(z, in[0], in[12]);
+        const double h3 = fma(x, in[1], in[11]);
+        const double h4 = fma(y, in[1], in[13]);
+        const double h5 = fma(z, in[1], in[14]);
+        const double h6 = fma(x, in[2], in[12]);
+        const double h7 = fma(y, in[2], in[14]);
+        const double h8 = fma(z, in[2], in[15]);
+        const double h9 = fma(x, in[3], in[13]);
+        const double h10 = fma(y, in[3], in[16]);
+        const double h11 = fma(z, in[3], in[17]);
+        const double h12 = fma(x, in[4], in[15]);
+        const double h13 = fma(y, in[4], in[18]);
+        const double h14 = fma(z, in[4], in[19]);
+        const double h15 = fma(x, in[5], in[14]);
+        const double h16 = fma(y, in[5], in[17]);
+        const double h17 = fma(z, in[5], in[18]);
+        const double h18 = fma(x, in[6], in[16]);
+        const double h19 = fma(y, in[6], in[20]);
+        const double h20 = fma(z, in[6], in[21]);
+        const double h21 = fma(x, in[7], in[17]);
+        const double h22 = fma(y, in[7], in[21]);
+        const double h23 = fma(z, in[7], in[22]);
+        const double h24 = fma(x, in[8], in[18]);
+        const double h25 = fma(y, in[8], in[22]);
+        const double h26 = fma(z, in[8], in[23]);
+        const double h27 = fma(x, in[9], in[19]);
+        const double h28 = fma(y, in[9], in[23]);
+        const double h29 = fma(z, in[9], in[24]);
+        out[0] = h0;
+        out[25] = h1;
+        out[50] = h2;
+        out[75] = h3;
+        out[100] = h4;
+        out[125] = h5;
+        out[150] = h6;
+        out[175] = h7;
+        out[200] = h8;
+        out[225] = h9;
+        out[250] = h10;
+        out[275] = h11;
+        out[300] = h12;
+        out[325] = h13;
+        out[350] = h14;
+        out[375] = h15;
+        out[400] = h16;
+        out[425] = h17;
+        out[450] = h18;
+        out[475] = h19;
+        out[500] = h20;
+        out[525] = h21;
+        out[550] = h22;
+        out[575] = h23;
+        out[600] = h24;
+        out[625] = h25;
+        out[650] = h26;
+        out[675] = h27;
+        out[700] = h28;
+        out[725] = h29;
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[0], in[10]);
+        const double h1 = fma(y, in[0], in[11]);
+        const double h2 = fma(z, in[0], in[12]);
+        const double h3 = fma(x, in[1], in[11]);
+        const double h4 = fma(y, in[1], in[13]);
+        const double h5 = fma(z, in[1], in[14]);
+        const double h6 = fma(x, in[2], in[12]);
+        const double h7 = fma(y, in[2], in[14]);
+        const double h8 = fma(z, in[2], in[15]);
+        const double h9 = fma(x, in[3], in[13]);
+        const double h10 = fma(y, in[3], in[16]);
+        const double h11 = fma(z, in[3], in[17]);
+        const double h12 = fma(x, in[4], in[15]);
+        const double h13 = fma(y, in[4], in[18]);
+        const double h14 = fma(z, in[4], in[19]);
+        const double h15 = fma(x, in[5], in[14]);
+        const double h16 = fma(y, in[5], in[17]);
+        const double h17 = fma(z, in[5], in[18]);
+        const double h18 = fma(x, in[6], in[16]);
+        const double h19 = fma(y, in[6], in[20]);
+        const double h20 = fma(z, in[6], in[21]);
+        const double h21 = fma(x, in[7], in[17]);
+        const double h22 = fma(y, in[7], in[21]);
+        const double h23 = fma(z, in[7], in[22]);
+        const double h24 = fma(x, in[8], in[18]);
+        const double h25 = fma(y, in[8], in[22]);
+        const double h26 = fma(z, in[8], in[23]);
+        const double h27 = fma(x, in[9], in[19]);
+        const double h28 = fma(y, in[9], in[23]);
+        const double h29 = fma(z, in[9], in[24]);
+        out[0] = h0 * (nrm * 0.2581988897471611);
+        out[1] = h1 * (nrm * 0.2581988897471611);
+        out[2] = h2 * (nrm * 0.2581988897471611);
+        out[3] = h3 * (nrm * 0.5773502691896258);
+        out[4] = h4 * (nrm * 0.5773502691896258);
+        out[5] = h5 * (nrm * 0.5773502691896258);
+        out[6] = h6 * (nrm * 0.5773502691896258);
+        out[7] = h7 * (nrm * 0.5773502691896258);
+        out[8] = h8 * (nrm * 0.5773502691896258);
+        out[9] = h9 * (nrm * 0.5773502691896258);
+        out[10] = h10 * (nrm * 0.5773502691896258);
+        out[11] = h11 * (nrm * 0.5773502691896258);
+        out[12] = h12 * (nrm * 0.5773502691896258);
+        out[13] = h13 * (nrm * 0.5773502691896258);
+        out[14] = h14 * (nrm * 0.5773502691896258);
+        out[15] = h15 * (nrm * 1.0);
+        out[16] = h16 * (nrm * 1.0);
+        out[17] = h17 * (nrm * 1.0);
+        out[18] = h18 * (nrm * 0.2581988897471611);
+        out[19] = h19 * (nrm * 0.2581988897471611);
+        out[20] = h20 * (nrm * 0.2581988897471611);
+        out[21] = h21 * (nrm * 0.5773502691896258);
+        out[22] = h22 * (nrm * 0.5773502691896258);
+        out[23] = h23 * (nrm * 0.5773502691896258);
+        out[24] = h24 * (nrm * 0.5773502691896258);
+        out[25] = h25 * (nrm * 0.5773502691896258);
+        out[26] = h26 * (nrm * 0.5773502691896258);
+        out[27] = h27 * (nrm * 0.2581988897471611);
+        out[28] = h28 * (nrm * 0.2581988897471611);
+        out[29] = h29 * (nrm * 0.2581988897471611);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_fpfp[625] = {
-    18, 273, 65553, 528, 131088, 65808, 783, 66063, 131343, 196623, 19, 274,
-    65554, 529, 65809, 131089, 784, 66064, 131344, 196624, 1039, 66319, 131599, 196879,
-    262159, 1293, 1548, 66828, 1803, 132363, 67083, 2058, 67338, 132618, 197898, 1294,
-    1549, 66829, 1804, 67084, 132364, 2059, 67339, 132619, 197899, 2314, 67594, 132874,
-    198154, 263434, 327693, 327948, 393228, 328203, 458763, 393483, 328458, 393738, 459018, 524298,
-    327694, 327949, 393229, 328204, 393484, 458764, 328459, 393739, 459019, 524299, 328714, 393994,
-    459274, 524554, 589834, 2568, 2823, 68103, 3078, 133638, 68358, 3333, 68613, 133893,
-    199173, 2569, 2824, 68104, 3079, 68359, 133639, 3334, 68614, 133894, 199174, 3589,
-    68869, 134149, 199429, 264709, 655368, 655623, 720903, 655878, 786438, 721158, 656133, 721413,
-    786693, 851973, 655369, 655624, 720904, 655879, 721159, 786439, 656134, 721414, 786694, 851974,
-    656389, 721669, 786949, 852229, 917509, 328968, 329223, 394503, 329478, 460038, 394758, 329733,
-    395013, 460293, 525573, 328969, 329224, 394504, 329479, 394759, 460039, 329734, 395014, 460294,
-    525574, 329989, 395269, 460549, 525829, 591109, 3843, 4098, 69378, 4353, 134913, 69633,
-    4608, 69888, 135168, 200448, 3844, 4099, 69379, 4354, 69634, 134914, 4609, 69889,
-    135169, 200449, 4864, 70144, 135424, 200704, 265984, 330243, 330498, 395778, 330753, 461313,
-    396033, 331008, 396288, 461568, 526848, 330244, 330499, 395779, 330754, 396034, 461314, 331009,
-    396289, 461569, 526849, 331264, 396544, 461824, 527104, 592384, 656643, 656898, 722178, 657153,
-    787713, 722433, 657408, 722688, 787968, 853248, 656644, 656899, 722179, 657154, 722434, 787714,
-    657409, 722689, 787969, 853249, 657664, 722944, 788224, 853504, 918784, 983043, 983298, 1048578,
-    983553, 1114113, 1048833, 983808, 1049088, 1114368, 1179648, 983044, 983299, 1048579, 983554, 1048834,
-    1114114, 983809, 1049089, 1114369, 1179649, 984064, 1049344, 1114624, 1179904, 1245184, 23, 278,
-    65558, 533, 131093, 65813, 788, 66068, 131348, 196628, 24, 279, 65559, 534,
-    65814, 131094, 789, 66069, 131349, 196629, 1044, 66324, 131604, 196884, 262164, 1298,
-    1553, 66833, 1808, 132368, 67088, 2063, 67343, 132623, 197903, 1299, 1554, 66834,
-    1809, 67089, 132369, 2064, 67344, 132624, 197904, 2319, 67599, 132879, 198159, 263439,
-    327698, 327953, 393233, 328208, 458768, 393488, 328463, 393743, 459023, 524303, 327699, 327954,
-    393234, 328209, 393489, 458769, 328464, 393744, 459024, 524304, 328719, 393999, 459279, 524559,
-    589839, 2573, 2828, 68108, 3083, 133643, 68363, 3338, 68618, 133898, 199178, 2574,
-    2829, 68109, 3084, 68364, 133644, 3339, 68619, 133899, 199179, 3594, 68874, 134154,
-    199434, 264714, 328973, 329228, 394508, 329483, 460043, 394763, 329738, 395018, 460298, 525578,
-    328974, 329229, 394509, 329484, 394764, 460044, 329739, 395019, 460299, 525579, 329994, 395274,
-    460554, 525834, 591114, 655373, 655628, 720908, 655883, 786443, 721163, 656138, 721418, 786698,
-    851978, 655374, 655629, 720909, 655884, 721164, 786444, 656139, 721419, 786699, 851979, 656394,
-    721674, 786954, 852234, 917514, 3848, 4103, 69383, 4358, 134918, 69638, 4613, 69893,
-    135173, 200453, 3849, 4104, 69384, 4359, 69639, 134919, 4614, 69894, 135174, 200454,
-    4869, 70149, 135429, 200709, 265989, 330248, 330503, 395783, 330758, 461318, 396038, 331013,
-    396293, 461573, 526853, 330249, 330504, 395784, 330759, 396039, 461319, 331014, 396294, 461574,
-    526854, 331269, 396549, 461829, 527109, 592389, 656648, 656903, 722183, 657158, 787718, 722438,
-    657413, 722693, 787973, 853253, 656649, 656904, 722184, 657159, 722439, 787719, 657414, 722694,
-    787974, 853254, 657669, 722949, 788229, 853509, 918789, 983048, 983303, 1048583, 983558, 1114118,
-    1048838, 983813, 1049093, 1114373, 1179653, 983049, 983304, 1048584, 983559, 1048839, 1114119, 983814,
-    1049094, 1114374, 1179654, 984069, 1049349, 1114629, 1179909, 1245189, 5123, 5378, 70658, 5633,
-    136193, 70913, 5888, 71168, 136448, 201728, 5124, 5379, 70659, 5634, 70914, 136194,
-    5889, 71169, 136449, 201729, 6144, 71424, 136704, 201984, 267264, 331523, 331778, 397058,
-    332033, 462593, 397313, 332288, 397568, 462848, 528128, 331524, 331779, 397059, 332034, 397314,
-    462594, 332289, 397569, 462849, 528129, 332544, 397824, 463104, 528384, 593664, 657923, 658178,
-    723458, 658433, 788993, 723713, 658688, 723968, 789248, 854528, 657924, 658179, 723459, 658434,
-    723714, 788994, 658689, 723969, 789249, 854529, 658944, 724224, 789504, 854784, 920064, 984323,
-    984578, 1049858, 984833, 1115393, 1050113, 985088, 1050368, 1115648, 1180928, 984324, 984579, 1049859,
-    984834, 1050114, 1115394, 985089, 1050369, 1115649, 1180929, 985344, 1050624, 1115904, 1181184, 1246464,
-    1310723, 1310978, 1376258, 1311233, 1441793, 1376513, 1311488, 1376768, 1442048, 1507328, 1310724, 1310979,
-    1376259, 1311234, 1376514, 1441794, 1311489, 1376769, 1442049, 1507329, 1311744, 1377024, 1442304, 1507584,
-    1572864,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_fpfp[31] = {
-    0, 2, 4, 6, 8, 10, 12, 14, 16, 18, 20, 22,
-    24, 26, 28, 30, 32, 34, 36, 38, 40, 42, 44, 46,
-    48, 50, 52, 54, 56, 58, 60,
-};
-__device__ const uint32_t kBraTerm_fpfp[60] = {
-    65792, 65546, 66048, 65547, 66304, 65548, 65793, 65547, 66049, 65549, 66305, 65550,
-    65794, 65548, 66050, 65550, 66306, 65551, 65795, 65549, 66051, 65552, 66307, 65553,
-    65796, 65551, 66052, 65554, 66308, 65555, 65797, 65550, 66053, 65553, 66309, 65554,
-    65798, 65552, 66054, 65556, 66310, 65557, 65799, 65553, 66055, 65557, 66311, 65558,
-    65800, 65554, 66056, 65558, 66312, 65559, 65801, 65555, 66057, 65559, 66313, 65560,
-};
-__device__ const uint16_t kKetOff_fpfp[31] = {
-    0, 2, 4, 6, 8, 10, 12, 14, 16, 18, 20, 22,
-    24, 26, 28, 30, 32, 34, 36, 38, 40, 42, 44, 46,
-    48, 50, 52, 54, 56, 58, 60,
-};
-__device__ const uint32_t kKetTerm_fpfp[60] = {
-    65792, 65546, 66048, 65547, 66304, 65548, 65793, 65547, 66049, 65549, 66305, 65550,
-    65794, 65548, 66050, 65550, 66306, 65551, 65795, 65549, 66051, 65552, 66307, 65553,
-    65796, 65551, 66052, 65554, 66308, 65555, 65797, 65550, 66053, 65553, 66309, 65554,
-    65798, 65552, 66054, 65556, 66310, 65557, 65799, 65553, 66055, 65557, 66311, 65558,
-    65800, 65554, 66056, 65558, 66312, 65559, 65801, 65555, 66057, 65559, 66313, 65560,
-};
 __device__ const double kNormAB_fpfp[30] = {
     0.2581988897471611, 0.2581988897471611, 0.2581988897471611, 0.5773502691896258,
     0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
@@ -138,24 +182,12 @@ __device__ const double kNormAB_fpfp[30] = {
     0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.2581988897471611,
     0.2581988897471611, 0.2581988897471611,
 };
-__device__ const double kNormCD_fpfp[30] = {
-    0.2581988897471611, 0.2581988897471611, 0.2581988897471611, 0.5773502691896258,
-    0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
-    0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
-    0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 1.0,
-    1.0, 1.0, 0.2581988897471611, 0.2581988897471611,
-    0.2581988897471611, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
-    0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.2581988897471611,
-    0.2581988897471611, 0.2581988897471611,
-};
-
 
 // column components cx | cy << 4 | cz << 8
 __device__ const uint16_t kCol_fpfp[25] = { 3, 18, 258, 33, 513, 273, 48, 288, 528, 768, 4, 19, 259, 34, 274, 514, 49, 289, 529, 769, 64, 304, 544, 784, 1024 };
 
 __device__ __forceinline__ RysClassTabs tabs_fpfp() {
-    return RysClassTabs{kBlk_fpfp, kBraOff_fpfp, kBraTerm_fpfp, kKetOff_fpfp, kKetTerm_fpfp,
-                        kNormAB_fpfp, kNormCD_fpfp, kCol_fpfp};
+    return RysClassTabs{kNormAB_fpfp, kCol_fpfp};
 }
 
 template <int MIXED>
@@ -173,9 +205,9 @@ static void rys_prepare_fpfp() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_fpfp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 73280);
-        cudaFuncSetAttribute(rys_queue_fpfp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 73280);
-        cudaFuncSetAttribute(rys_bound_kernel_fpfp, cudaFuncAttributeMaxDynamicSharedMemorySize, 73280);
+        cudaFuncSetAttribute(rys_queue_fpfp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 53760);
+        cudaFuncSetAttribute(rys_queue_fpfp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 53760);
+        cudaFuncSetAttribute(rys_bound_kernel_fpfp, cudaFuncAttributeMaxDynamicSharedMemorySize, 53760);
         done[dev] = true;
     }
 }
@@ -186,16 +218,16 @@ void launch_rys_fpfp(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_fpfp();
     constexpr int ng = 128 / C_fpfp::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_fpfp<1><<<grid, 128, 73280, s>>>(Q, R);
-    else rys_queue_fpfp<0><<<grid, 128, 73280, s>>>(Q, R);
+    if (mixed) rys_queue_fpfp<1><<<grid, 128, 53760, s>>>(Q, R);
+    else rys_queue_fpfp<0><<<grid, 128, 53760, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_fpfp(int mixed) {
     rys_prepare_fpfp();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fpfp<1>, 128, 73280);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fpfp<0>, 128, 73280);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fpfp<1>, 128, 53760);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fpfp<0>, 128, 53760);
     return n;
 }
 
@@ -204,7 +236,7 @@ void launch_rys_bound_fpfp(const PairTab &P, const RysTab &R, int p0, int np, do
     if (np <= 0) return;
     rys_prepare_fpfp();
     constexpr int ng = 128 / C_fpfp::G;
-    rys_bound_kernel_fpfp<<<(np + ng - 1) / ng, 128, 73280, s>>>(P, R, p0, np, pbound, qout, full);
+    rys_bound_kernel_fpfp<<<(np + ng - 1) / ng, 128, 53760, s>>>(P, R, p0, np, pbound, qout, full);
 }
 
 }  // namespace molints

@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (fp|ps).  Do not edit.
-// roots 3, block 25 x 3, outputs 30 x 3, group 32 threads,
-// 10 primitive quartets per batch, 1 slot(s), 3 accumulators per thread, 30080 B shared per block.
+// roots 3, block 25 x 3, outputs 30 x 3, group 32 threads, 5 ket pairs a round,
+// 2 primitive quartets per ket pair and batch, 29760 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,43 +11,110 @@ struct C_fpps {
     static constexpr int NA = 25, NC = 3, NBLK = 75;
     static constexpr int NB = 3, ND = 1;
     static constexpr int NAB = 30, NCD = 3;
-    static constexpr int G = 32, NPB = 10, NSLOT = 1, ACC = 3;
-    static constexpr int S = 10;
-    static constexpr int SMEM_GROUP = 940;
-    static constexpr bool COL = false;
+    static constexpr int G = 32, W = 5, H = 2, PB = 2;
+    static constexpr int S = 10, SI = 31, NCP = 3, NCDP = 3;
+    static constexpr int SMEM_GROUP = 930;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
-    __device__ __forceinline__ static void col_update(const T *, const T *, const T *, A *) {}
+    __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
+        acc[0] = fma(x[3] * y[0], z[0], acc[0]);
+        acc[1] = fma(x[2] * y[1], z[0], acc[1]);
+        acc[2] = fma(x[2] * y[0], z[1], acc[2]);
+        acc[3] = fma(x[1] * y[2], z[0], acc[3]);
+        acc[4] = fma(x[1] * y[0], z[2], acc[4]);
+        acc[5] = fma(x[1] * y[1], z[1], acc[5]);
+        acc[6] = fma(x[0] * y[3], z[0], acc[6]);
+        acc[7] = fma(x[0] * y[2], z[1], acc[7]);
+        acc[8] = fma(x[0] * y[1], z[2], acc[8]);
+        acc[9] = fma(x[0] * y[0], z[3], acc[9]);
+        acc[10] = fma(x[4] * y[0], z[0], acc[10]);
+        acc[11] = fma(x[3] * y[1], z[0], acc[11]);
+        acc[12] = fma(x[3] * y[0], z[1], acc[12]);
+        acc[13] = fma(x[2] * y[2], z[0], acc[13]);
+        acc[14] = fma(x[2] * y[1], z[1], acc[14]);
+        acc[15] = fma(x[2] * y[0], z[2], acc[15]);
+        acc[16] = fma(x[1] * y[3], z[0], acc[16]);
+        acc[17] = fma(x[1] * y[2], z[1], acc[17]);
+        acc[18] = fma(x[1] * y[1], z[2], acc[18]);
+        acc[19] = fma(x[1] * y[0], z[3], acc[19]);
+        acc[20] = fma(x[0] * y[4], z[0], acc[20]);
+        acc[21] = fma(x[0] * y[3], z[1], acc[21]);
+        acc[22] = fma(x[0] * y[2], z[2], acc[22]);
+        acc[23] = fma(x[0] * y[1], z[3], acc[23]);
+        acc[24] = fma(x[0] * y[0], z[4], acc[24]);
+    }
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[0], in[10]);
+        const double h1 = fma(y, in[0], in[11]);
+        const double h2 = fma(z, in[0], in[12]);
+        const double h3 = fma(x, in[1], in[11]);
+        const double h4 = fma(y, in[1], in[13]);
+        const double h5 = fma(z, in[1], in[14]);
+        const double h6 = fma(x, in[2], in[12]);
+        const double h7 = fma(y, in[2], in[14]);
+        const double h8 = fma(z, in[2], in[15]);
+        const double h9 = fma(x, in[3], in[13]);
+        const double h10 = fma(y, in[3], in[16]);
+        const double h11 = fma(z, in[3], in[17]);
+        const double h12 = fma(x, in[4], in[15]);
+        const double h13 = fma(y, in[4], in[18]);
+        const double h14 = fma(z, in[4], in[19]);
+        const double h15 = fma(x, in[5], in[14]);
+        const double h16 = fma(y, in[5], in[17]);
+        const double h17 = fma(z, in[5], in[18]);
+        const double h18 = fma(x, in[6], in[16]);
+        const double h19 = fma(y, in[6], in[20]);
+        const double h20 = fma(z, in[6], in[21]);
+        const double h21 = fma(x, in[7], in[17]);
+        const double h22 = fma(y, in[7], in[21]);
+        const double h23 = fma(z, in[7], in[22]);
+        const double h24 = fma(x, in[8], in[18]);
+        const double h25 = fma(y, in[8], in[22]);
+        const double h26 = fma(z, in[8], in[23]);
+        const double h27 = fma(x, in[9], in[19]);
+        const double h28 = fma(y, in[9], in[23]);
+        const double h29 = fma(z, in[9], in[24]);
+        out[0] = h0;
+        out[3] = h1;
+        out[6] = h2;
+        out[9] = h3;
+        out[12] = h4;
+        out[15] = h5;
+        out[18] = h6;
+        out[21] = h7;
+        out[24] = h8;
+        out[27] = h9;
+        out[30] = h10;
+        out[33] = h11;
+        out[36] = h12;
+        out[39] = h13;
+        out[42] = h14;
+        out[45] = h15;
+        out[48] = h16;
+        out[51] = h17;
+        out[54] = h18;
+        out[57] = h19;
+        out[60] = h20;
+        out[63] = h21;
+        out[66] = h22;
+        out[69] = h23;
+        out[72] = h24;
+        out[75] = h25;
+        out[78] = h26;
+        out[81] = h27;
+        out[84] = h28;
+        out[87] = h29;
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        out[0] = in[0] * (nrm * 1.0);
+        out[1] = in[1] * (nrm * 1.0);
+        out[2] = in[2] * (nrm * 1.0);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_fpps[75] = {
-    7, 262, 65542, 517, 772, 66052, 131077, 131332, 196612, 1027, 1282, 66562,
-    262147, 262402, 327682, 131587, 131842, 197122, 1537, 1792, 67072, 132097, 132352, 197632,
-    262657, 262912, 328192, 393217, 393472, 458752, 9, 264, 65544, 519, 774, 66054,
-    131079, 131334, 196614, 1029, 1284, 66564, 131589, 131844, 197124, 262149, 262404, 327684,
-    1539, 1794, 67074, 132099, 132354, 197634, 262659, 262914, 328194, 393219, 393474, 458754,
-    2049, 2304, 67584, 132609, 132864, 198144, 263169, 263424, 328704, 393729, 393984, 459264,
-    524289, 524544, 589824,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_fpps[31] = {
-    0, 2, 4, 6, 8, 10, 12, 14, 16, 18, 20, 22,
-    24, 26, 28, 30, 32, 34, 36, 38, 40, 42, 44, 46,
-    48, 50, 52, 54, 56, 58, 60,
-};
-__device__ const uint32_t kBraTerm_fpps[60] = {
-    65792, 65546, 66048, 65547, 66304, 65548, 65793, 65547, 66049, 65549, 66305, 65550,
-    65794, 65548, 66050, 65550, 66306, 65551, 65795, 65549, 66051, 65552, 66307, 65553,
-    65796, 65551, 66052, 65554, 66308, 65555, 65797, 65550, 66053, 65553, 66309, 65554,
-    65798, 65552, 66054, 65556, 66310, 65557, 65799, 65553, 66055, 65557, 66311, 65558,
-    65800, 65554, 66056, 65558, 66312, 65559, 65801, 65555, 66057, 65559, 66313, 65560,
-};
-__device__ const uint16_t kKetOff_fpps[4] = {
-    0, 1, 2, 3,
-};
-__device__ const uint32_t kKetTerm_fpps[3] = {
-    65536, 65537, 65538,
-};
 __device__ const double kNormAB_fpps[30] = {
     0.2581988897471611, 0.2581988897471611, 0.2581988897471611, 0.5773502691896258,
     0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
@@ -58,14 +125,12 @@ __device__ const double kNormAB_fpps[30] = {
     0.5773502691896258, 0.5773502691896258, 0.5773502691896258, 0.2581988897471611,
     0.2581988897471611, 0.2581988897471611,
 };
-__device__ const double kNormCD_fpps[3] = {
-    1.0, 1.0, 1.0,
-};
 
+// column components cx | cy << 4 | cz << 8
+__device__ const uint16_t kCol_fpps[3] = { 1, 16, 256 };
 
 __device__ __forceinline__ RysClassTabs tabs_fpps() {
-    return RysClassTabs{kBlk_fpps, kBraOff_fpps, kBraTerm_fpps, kKetOff_fpps, kKetTerm_fpps,
-                        kNormAB_fpps, kNormCD_fpps, nullptr};
+    return RysClassTabs{kNormAB_fpps, kCol_fpps};
 }
 
 template <int MIXED>
@@ -78,8 +143,8 @@ static void rys_prepare_fpps() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_fpps<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 30080);
-        cudaFuncSetAttribute(rys_queue_fpps<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 30080);
+        cudaFuncSetAttribute(rys_queue_fpps<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 29760);
+        cudaFuncSetAttribute(rys_queue_fpps<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 29760);
 
         done[dev] = true;
     }
@@ -91,16 +156,16 @@ void launch_rys_fpps(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_fpps();
     constexpr int ng = 128 / C_fpps::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_fpps<1><<<grid, 128, 30080, s>>>(Q, R);
-    else rys_queue_fpps<0><<<grid, 128, 30080, s>>>(Q, R);
+    if (mixed) rys_queue_fpps<1><<<grid, 128, 29760, s>>>(Q, R);
+    else rys_queue_fpps<0><<<grid, 128, 29760, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_fpps(int mixed) {
     rys_prepare_fpps();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fpps<1>, 128, 30080);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fpps<0>, 128, 30080);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fpps<1>, 128, 29760);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fpps<0>, 128, 29760);
     return n;
 }
 

@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (fs|ds).  Do not edit.
-// roots 3, block 10 x 6, outputs 10 x 6, group 32 threads,
-// 10 primitive quartets per batch, 1 slot(s), 2 accumulators per thread, 35840 B shared per block.
+// roots 3, block 10 x 6, outputs 10 x 6, group 32 threads, 5 ket pairs a round,
+// 2 primitive quartets per ket pair and batch, 35520 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,49 +11,59 @@ struct C_fsds {
     static constexpr int NA = 10, NC = 6, NBLK = 60;
     static constexpr int NB = 1, ND = 1;
     static constexpr int NAB = 10, NCD = 6;
-    static constexpr int G = 32, NPB = 10, NSLOT = 1, ACC = 2;
-    static constexpr int S = 12;
-    static constexpr int SMEM_GROUP = 1120;
-    static constexpr bool COL = false;
+    static constexpr int G = 32, W = 5, H = 1, PB = 2;
+    static constexpr int S = 12, SI = 37, NCP = 7, NCDP = 7;
+    static constexpr int SMEM_GROUP = 1110;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
-    __device__ __forceinline__ static void col_update(const T *, const T *, const T *, A *) {}
+    __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
+        acc[0] = fma(x[3] * y[0], z[0], acc[0]);
+        acc[1] = fma(x[2] * y[1], z[0], acc[1]);
+        acc[2] = fma(x[2] * y[0], z[1], acc[2]);
+        acc[3] = fma(x[1] * y[2], z[0], acc[3]);
+        acc[4] = fma(x[1] * y[0], z[2], acc[4]);
+        acc[5] = fma(x[1] * y[1], z[1], acc[5]);
+        acc[6] = fma(x[0] * y[3], z[0], acc[6]);
+        acc[7] = fma(x[0] * y[2], z[1], acc[7]);
+        acc[8] = fma(x[0] * y[1], z[2], acc[8]);
+        acc[9] = fma(x[0] * y[0], z[3], acc[9]);
+    }
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        out[0] = in[0];
+        out[7] = in[1];
+        out[14] = in[2];
+        out[21] = in[3];
+        out[28] = in[4];
+        out[35] = in[5];
+        out[42] = in[6];
+        out[49] = in[7];
+        out[56] = in[8];
+        out[63] = in[9];
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        out[0] = in[0] * (nrm * 0.5773502691896258);
+        out[1] = in[1] * (nrm * 1.0);
+        out[2] = in[2] * (nrm * 1.0);
+        out[3] = in[3] * (nrm * 0.5773502691896258);
+        out[4] = in[4] * (nrm * 1.0);
+        out[5] = in[5] * (nrm * 0.5773502691896258);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_fsds[60] = {
-    11, 266, 65546, 521, 65801, 131081, 776, 1031, 66311, 1286, 66566, 131846,
-    196616, 196871, 262151, 197126, 262406, 327686, 1541, 1796, 67076, 2051, 67331, 132611,
-    393221, 393476, 458756, 393731, 459011, 524291, 197381, 197636, 262916, 197891, 263171, 328451,
-    2306, 2561, 67841, 2816, 68096, 133376, 198146, 198401, 263681, 198656, 263936, 329216,
-    393986, 394241, 459521, 394496, 459776, 525056, 589826, 590081, 655361, 590336, 655616, 720896,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_fsds[11] = {
-    0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10,
-};
-__device__ const uint32_t kBraTerm_fsds[10] = {
-    65536, 65537, 65538, 65539, 65540, 65541, 65542, 65543, 65544, 65545,
-};
-__device__ const uint16_t kKetOff_fsds[7] = {
-    0, 1, 2, 3, 4, 5, 6,
-};
-__device__ const uint32_t kKetTerm_fsds[6] = {
-    65536, 65537, 65538, 65539, 65540, 65541,
-};
 __device__ const double kNormAB_fsds[10] = {
     0.2581988897471611, 0.5773502691896258, 0.5773502691896258, 0.5773502691896258,
     0.5773502691896258, 1.0, 0.2581988897471611, 0.5773502691896258,
     0.5773502691896258, 0.2581988897471611,
 };
-__device__ const double kNormCD_fsds[6] = {
-    0.5773502691896258, 1.0, 1.0, 0.5773502691896258,
-    1.0, 0.5773502691896258,
-};
 
+// column components cx | cy << 4 | cz << 8
+__device__ const uint16_t kCol_fsds[6] = { 2, 17, 257, 32, 272, 512 };
 
 __device__ __forceinline__ RysClassTabs tabs_fsds() {
-    return RysClassTabs{kBlk_fsds, kBraOff_fsds, kBraTerm_fsds, kKetOff_fsds, kKetTerm_fsds,
-                        kNormAB_fsds, kNormCD_fsds, nullptr};
+    return RysClassTabs{kNormAB_fsds, kCol_fsds};
 }
 
 template <int MIXED>
@@ -66,8 +76,8 @@ static void rys_prepare_fsds() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_fsds<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 35840);
-        cudaFuncSetAttribute(rys_queue_fsds<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 35840);
+        cudaFuncSetAttribute(rys_queue_fsds<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 35520);
+        cudaFuncSetAttribute(rys_queue_fsds<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 35520);
 
         done[dev] = true;
     }
@@ -79,16 +89,16 @@ void launch_rys_fsds(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_fsds();
     constexpr int ng = 128 / C_fsds::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_fsds<1><<<grid, 128, 35840, s>>>(Q, R);
-    else rys_queue_fsds<0><<<grid, 128, 35840, s>>>(Q, R);
+    if (mixed) rys_queue_fsds<1><<<grid, 128, 35520, s>>>(Q, R);
+    else rys_queue_fsds<0><<<grid, 128, 35520, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_fsds(int mixed) {
     rys_prepare_fsds();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fsds<1>, 128, 35840);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fsds<0>, 128, 35840);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fsds<1>, 128, 35520);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fsds<0>, 128, 35520);
     return n;
 }
 

@@ -1,6 +1,6 @@
 // Generated by gen_rys.py -- Rys class (pp|pp).  Do not edit.
-// roots 3, block 9 x 9, outputs 9 x 9, group 32 threads,
-// 10 primitive quartets per batch, 1 slot(s), 3 accumulators per thread, 27200 B shared per block.
+// roots 3, block 9 x 9, outputs 9 x 9, group 32 threads, 3 ket pairs a round,
+// 3 primitive quartets per ket pair and batch, 23328 B shared per block.
 #include "../rys_common.cuh"
 
 namespace molints {
@@ -11,54 +11,78 @@ struct C_pppp {
     static constexpr int NA = 9, NC = 9, NBLK = 81;
     static constexpr int NB = 3, ND = 3;
     static constexpr int NAB = 9, NCD = 9;
-    static constexpr int G = 32, NPB = 10, NSLOT = 1, ACC = 3;
-    static constexpr int S = 9;
-    static constexpr int SMEM_GROUP = 850;
-    static constexpr bool COL = false;
+    static constexpr int G = 32, W = 3, H = 1, PB = 3;
+    static constexpr int S = 9, SI = 27, NCP = 9, NCDP = 9;
+    static constexpr int SMEM_GROUP = 729;
+    // stage 2: acc[row] += x[ax] y[ay] z[az] for the column's table columns
     template <typename T, typename A>
-    __device__ __forceinline__ static void col_update(const T *, const T *, const T *, A *) {}
+    __device__ __forceinline__ static void col_update(const T *x, const T *y, const T *z, A *acc) {
+        acc[0] = fma(x[1] * y[0], z[0], acc[0]);
+        acc[1] = fma(x[0] * y[1], z[0], acc[1]);
+        acc[2] = fma(x[0] * y[0], z[1], acc[2]);
+        acc[3] = fma(x[2] * y[0], z[0], acc[3]);
+        acc[4] = fma(x[1] * y[1], z[0], acc[4]);
+        acc[5] = fma(x[1] * y[0], z[1], acc[5]);
+        acc[6] = fma(x[0] * y[2], z[0], acc[6]);
+        acc[7] = fma(x[0] * y[1], z[1], acc[7]);
+        acc[8] = fma(x[0] * y[0], z[2], acc[8]);
+    }
+    // bra HRR of one column (row stride NCP), ket HRR of one row times the component norms
+    __device__ __forceinline__ static void bra_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[0], in[3]);
+        const double h1 = fma(y, in[0], in[4]);
+        const double h2 = fma(z, in[0], in[5]);
+        const double h3 = fma(x, in[1], in[4]);
+        const double h4 = fma(y, in[1], in[6]);
+        const double h5 = fma(z, in[1], in[7]);
+        const double h6 = fma(x, in[2], in[5]);
+        const double h7 = fma(y, in[2], in[7]);
+        const double h8 = fma(z, in[2], in[8]);
+        out[0] = h0;
+        out[9] = h1;
+        out[18] = h2;
+        out[27] = h3;
+        out[36] = h4;
+        out[45] = h5;
+        out[54] = h6;
+        out[63] = h7;
+        out[72] = h8;
+    }
+    __device__ __forceinline__ static void ket_hrr(const double *__restrict__ in, double x, double y, double z, double nrm, double *__restrict__ out) {
+        (void)x; (void)y; (void)z; (void)nrm;
+        const double h0 = fma(x, in[0], in[3]);
+        const double h1 = fma(y, in[0], in[4]);
+        const double h2 = fma(z, in[0], in[5]);
+        const double h3 = fma(x, in[1], in[4]);
+        const double h4 = fma(y, in[1], in[6]);
+        const double h5 = fma(z, in[1], in[7]);
+        const double h6 = fma(x, in[2], in[5]);
+        const double h7 = fma(y, in[2], in[7]);
+        const double h8 = fma(z, in[2], in[8]);
+        out[0] = h0 * (nrm * 1.0);
+        out[1] = h1 * (nrm * 1.0);
+        out[2] = h2 * (nrm * 1.0);
+        out[3] = h3 * (nrm * 1.0);
+        out[4] = h4 * (nrm * 1.0);
+        out[5] = h5 * (nrm * 1.0);
+        out[6] = h6 * (nrm * 1.0);
+        out[7] = h7 * (nrm * 1.0);
+        out[8] = h8 * (nrm * 1.0);
+    }
 };
 
-// block entry (row, col) -> 2-D table offsets x | y << 8 | z << 16
-__device__ const uint32_t kBlk_pppp[81] = {
-    4, 259, 65539, 5, 260, 65540, 515, 65795, 131075, 769, 1024, 66304,
-    770, 1025, 66305, 1280, 66560, 131840, 196609, 196864, 262144, 196610, 196865, 262145,
-    197120, 262400, 327680, 7, 262, 65542, 8, 263, 65543, 518, 65798, 131078,
-    772, 1027, 66307, 773, 1028, 66308, 1283, 66563, 131843, 196612, 196867, 262147,
-    196613, 196868, 262148, 197123, 262403, 327683, 1537, 1792, 67072, 1538, 1793, 67073,
-    2048, 67328, 132608, 197377, 197632, 262912, 197378, 197633, 262913, 197888, 263168, 328448,
-    393217, 393472, 458752, 393218, 393473, 458753, 393728, 459008, 524288,
-};
-// HRR terms: block index | monomial << 8 | binomial << 16, per output pair
-__device__ const uint16_t kBraOff_pppp[10] = {
-    0, 2, 4, 6, 8, 10, 12, 14, 16, 18,
-};
-__device__ const uint32_t kBraTerm_pppp[18] = {
-    65792, 65539, 66048, 65540, 66304, 65541, 65793, 65540, 66049, 65542, 66305, 65543,
-    65794, 65541, 66050, 65543, 66306, 65544,
-};
-__device__ const uint16_t kKetOff_pppp[10] = {
-    0, 2, 4, 6, 8, 10, 12, 14, 16, 18,
-};
-__device__ const uint32_t kKetTerm_pppp[18] = {
-    65792, 65539, 66048, 65540, 66304, 65541, 65793, 65540, 66049, 65542, 66305, 65543,
-    65794, 65541, 66050, 65543, 66306, 65544,
-};
 __device__ const double kNormAB_pppp[9] = {
     1.0, 1.0, 1.0, 1.0,
     1.0, 1.0, 1.0, 1.0,
     1.0,
 };
-__device__ const double kNormCD_pppp[9] = {
-    1.0, 1.0, 1.0, 1.0,
-    1.0, 1.0, 1.0, 1.0,
-    1.0,
-};
 
+// column components cx | cy << 4 | cz << 8
+__device__ const uint16_t kCol_pppp[9] = { 1, 16, 256, 2, 17, 257, 32, 272, 512 };
 
 __device__ __forceinline__ RysClassTabs tabs_pppp() {
-    return RysClassTabs{kBlk_pppp, kBraOff_pppp, kBraTerm_pppp, kKetOff_pppp, kKetTerm_pppp,
-                        kNormAB_pppp, kNormCD_pppp, nullptr};
+    return RysClassTabs{kNormAB_pppp, kCol_pppp};
 }
 
 template <int MIXED>
@@ -76,9 +100,9 @@ static void rys_prepare_pppp() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(rys_queue_pppp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 27200);
-        cudaFuncSetAttribute(rys_queue_pppp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 27200);
-        cudaFuncSetAttribute(rys_bound_kernel_pppp, cudaFuncAttributeMaxDynamicSharedMemorySize, 27200);
+        cudaFuncSetAttribute(rys_queue_pppp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 23328);
+        cudaFuncSetAttribute(rys_queue_pppp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 23328);
+        cudaFuncSetAttribute(rys_bound_kernel_pppp, cudaFuncAttributeMaxDynamicSharedMemorySize, 23328);
         done[dev] = true;
     }
 }
@@ -89,16 +113,16 @@ void launch_rys_pppp(const EriQueue &Q, const RysTab &R, int mixed, int grid_max
     rys_prepare_pppp();
     constexpr int ng = 128 / C_pppp::G;
     const int grid = (int)std::min<long long>(grid_max, ((long long)Q.nchunks + ng - 1) / ng);
-    if (mixed) rys_queue_pppp<1><<<grid, 128, 27200, s>>>(Q, R);
-    else rys_queue_pppp<0><<<grid, 128, 27200, s>>>(Q, R);
+    if (mixed) rys_queue_pppp<1><<<grid, 128, 23328, s>>>(Q, R);
+    else rys_queue_pppp<0><<<grid, 128, 23328, s>>>(Q, R);
 }
 
 // Resident blocks of 128 threads per SM for the queue kernel (sizes the persistent grid).
 int occupancy_rys_pppp(int mixed) {
     rys_prepare_pppp();
     int n = 0;
-    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_pppp<1>, 128, 27200);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_pppp<0>, 128, 27200);
+    if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_pppp<1>, 128, 23328);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_pppp<0>, 128, 23328);
     return n;
 }
 
@@ -107,7 +131,7 @@ void launch_rys_bound_pppp(const PairTab &P, const RysTab &R, int p0, int np, do
     if (np <= 0) return;
     rys_prepare_pppp();
     constexpr int ng = 128 / C_pppp::G;
-    rys_bound_kernel_pppp<<<(np + ng - 1) / ng, 128, 27200, s>>>(P, R, p0, np, pbound, qout, full);
+    rys_bound_kernel_pppp<<<(np + ng - 1) / ng, 128, 23328, s>>>(P, R, p0, np, pbound, qout, full);
 }
 
 }  // namespace molints

@@ -1348,14 +1348,16 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
         int ci = 0, items = 0;
         for (int x = 0; x < kNumPairClasses; ++x)
             for (int y = 0; y <= x; ++y, ++ci) {
-                const bool hgp = p->method[x][y] != MOLINTS_METHOD_RYS;
+                // lane-split queues: the HGP kernels', and the Rys kernels' of small blocks
+                const bool rys = p->method[x][y] == MOLINTS_METHOD_RYS;
+                const bool hgp = !rys || kRysPrimCost[x][y] > 0.0f;
                 const int lsum = kPairClassLa[x] + kPairClassLb[x] + kPairClassLa[y] + kPairClassLb[y];
                 S.item_base[ci] = items;
                 S.cx[ci] = x;
                 S.cy[ci] = y;
                 S.hgp[ci] = hgp;
                 S.width[ci] = hgp ? 32 * hgp_widen : rys_width(x, y) * widen;
-                S.pcost[ci] = (double)kEriPrimCost[x][y];
+                S.pcost[ci] = (double)(rys ? kRysPrimCost[x][y] : kEriPrimCost[x][y]);
                 S.w[ci] = 1.0 + lsum * lsum;
                 items += cls_start[x + 1] - cls_start[x];
             }
@@ -1902,8 +1904,9 @@ static int plan_enqueue(molints_plan *p, double *out_device, bool timing, JKOut 
             Q.chunk_slot = p->chunk_slot + p->q_off[x][y];
             Q.region = p->g_region + ((size_t)x * kNumPairClasses + y) * p->nmol * kRegionFields;
         }
-        // HGP: one warp per chunk, four per block; Rys: the launcher divides by its groups/block
-        const int grid = rys ? occ * ctx->num_sms
+        // lane-split: one warp per chunk, four per block; Rys groups: the launcher divides by its
+        // groups per block
+        const int grid = rys && !(kRysPrimCost[x][y] > 0.0f) ? occ * ctx->num_sms
                              : (int)std::min<long long>((long long)occ * ctx->num_sms, (Q.nchunks + 3) / 4);
         const char *name = rys ? kRysNames[x][y] : kEriNames[x][y];
         if (int rc = mark(launches, name, 0, st)) return rc;
