@@ -51,6 +51,9 @@ MIXED_MIN_VRR = 40
 # chunk's blocks into dynamic shared memory (4 warps x 32 blocks x 8 B each: up to 162 KB) and
 # the warp copies them to the scratch as one contiguous run
 STAGE_MAX_OUT = 162
+# J/K digestion: blocks of at most this many outputs are digested from registers; larger ones sit in
+# local memory, read by a loop over A's components
+JK_UNROLL_MAX_OUT = 36
 
 
 # ------------------------------------------------------------------ AO tables
@@ -540,6 +543,76 @@ __device__ __forceinline__ void quartet_{tag}(const PairTab &P, const BoysTab &B
     }}
     hrr_{tag}(P, p, q, acc, res);
 }}"""
+    # J/K digestion: loops over A's components (unrolled for small blocks, so that res stays in
+    # registers), the rest unrolled
+    body = []
+    for jb in range(nb):
+        for ic in range(nc):
+            for jd in range(nd):
+                body += [f"        {{ const double v = f * res[(i * {nb} + {jb}) * {nc * nd} + {ic * nd + jd}];",
+                         f"          jab[i * {nb} + {jb}] = fma(dcd[{ic * nd + jd}], v, jab[i * {nb} + {jb}]);",
+                         f"          jcd[{ic * nd + jd}] = fma(dab[{jb}], v, jcd[{ic * nd + jd}]);",
+                         f"          kac[{ic}] = fma(dbd[{jb * nd + jd}], v, kac[{ic}]);",
+                         f"          kad[{jd}] = fma(dbc[{jb * nc + ic}], v, kad[{jd}]);",
+                         f"          kbc[{jb * nc + ic}] = fma(dad[{jd}], v, kbc[{jb * nc + ic}]);",
+                         f"          kbd[{jb * nd + jd}] = fma(dac[{ic}], v, kbd[{jb * nd + jd}]); }}"]
+    jk_body = "\n".join(body)
+    jk_fn = f"""// The quartet's share of J and K (molints_plan_jk, eri_common.cuh): every integral of the block,
+// times f, into one orientation of each target; J_ab stays in the lane (one bra pair per chunk).
+__device__ __forceinline__ void jk_{tag}(const JKOut &jk, const int4 ib_, const int4 ik_, double f,
+                                         const double *__restrict__ res, double *__restrict__ jab) {{
+    const long long n = jk.n;
+    const double *__restrict__ D = jk.D;
+    const double *__restrict__ Db = D + ib_.w * n, *__restrict__ Dc = D + ik_.z * n;
+    double dcd[{nc * nd}], dbc[{nb * nc}], dbd[{nb * nd}], jcd[{nc * nd}], kbc[{nb * nc}], kbd[{nb * nd}];
+#pragma unroll
+    for (int k = 0; k < {nc}; ++k)
+#pragma unroll
+        for (int l = 0; l < {nd}; ++l) {{
+            dcd[k * {nd} + l] = __ldg(&Dc[k * n + ik_.w + l]);
+            jcd[k * {nd} + l] = 0.0;
+        }}
+#pragma unroll
+    for (int j = 0; j < {nb}; ++j) {{
+#pragma unroll
+        for (int k = 0; k < {nc}; ++k) {{
+            dbc[j * {nc} + k] = __ldg(&Db[j * n + ik_.z + k]);
+            kbc[j * {nc} + k] = 0.0;
+        }}
+#pragma unroll
+        for (int l = 0; l < {nd}; ++l) {{
+            dbd[j * {nd} + l] = __ldg(&Db[j * n + ik_.w + l]);
+            kbd[j * {nd} + l] = 0.0;
+        }}
+    }}
+#pragma unroll {na if nout <= JK_UNROLL_MAX_OUT else 1}
+    for (int i = 0; i < {na}; ++i) {{
+        const double *__restrict__ Da = D + (ib_.z + i) * n;
+        double dab[{nb}], dac[{nc}], dad[{nd}], kac[{nc}], kad[{nd}];
+#pragma unroll
+        for (int j = 0; j < {nb}; ++j) dab[j] = __ldg(&Da[ib_.w + j]);
+#pragma unroll
+        for (int k = 0; k < {nc}; ++k) {{ dac[k] = __ldg(&Da[ik_.z + k]); kac[k] = 0.0; }}
+#pragma unroll
+        for (int l = 0; l < {nd}; ++l) {{ dad[l] = __ldg(&Da[ik_.w + l]); kad[l] = 0.0; }}
+{jk_body}
+#pragma unroll
+        for (int k = 0; k < {nc}; ++k) atomicAdd(&jk.K[(ib_.z + i) * n + ik_.z + k], kac[k]);
+#pragma unroll
+        for (int l = 0; l < {nd}; ++l) atomicAdd(&jk.K[(ib_.z + i) * n + ik_.w + l], kad[l]);
+    }}
+#pragma unroll
+    for (int j = 0; j < {nb}; ++j) {{
+#pragma unroll
+        for (int k = 0; k < {nc}; ++k) atomicAdd(&jk.K[(ib_.w + j) * n + ik_.z + k], kbc[j * {nc} + k]);
+#pragma unroll
+        for (int l = 0; l < {nd}; ++l) atomicAdd(&jk.K[(ib_.w + j) * n + ik_.w + l], kbd[j * {nd} + l]);
+    }}
+#pragma unroll
+    for (int k = 0; k < {nc}; ++k)
+#pragma unroll
+        for (int l = 0; l < {nd}; ++l) atomicAdd(&jk.J[(ik_.z + k) * n + ik_.w + l], 2.0 * jcd[k * {nd} + l]);
+}}"""
     if rys:
         head = (f"// Generated by gen_rys.py -- Rys class ({tag[0]}{tag[1]}|{tag[2]}{tag[3]}).  Do not edit.\n"
                 f"// roots {M // 2 + 1}, contracted block: {nacc}, outputs: {nout}: a lane-split kernel, the lanes' primitive quartets by\n"
@@ -590,18 +663,7 @@ __device__ __forceinline__ void store_{tag}(double *__restrict__ out, const int4
 {store_code}
 }}
 
-// The quartet's unique integrals digested into J and K (molints_plan_jk) instead of stored.
-__device__ __noinline__ void jk_{tag}(const JKOut &jk, const int4 ib_, const int4 ik_, bool same,
-                                      const double *__restrict__ res) {{
-    const bool dab = ib_.z == ib_.w, dcd = ik_.z == ik_.w;
-    for (int x = 0; x < {nout}; ++x) {{
-        const int ia = x / {nb * nc * nd}, ibb = (x / {nc * nd}) % {nb}, ic = (x / {nd}) % {nc}, id = x % {nd};
-        if ((dab && ia < ibb) || (dcd && ic < id)) continue;
-        const int i = ib_.z + ia, j = ib_.w + ibb, k = ik_.z + ic, l = ik_.w + id;
-        if (same && pair_index(i, j) < pair_index(k, l)) continue;
-        jk_add(jk, i, j, k, l, res[x]);
-    }}
-}}
+{jk_fn}
 
 // Persistent work-queue kernel: each warp takes chunks (one bra pair, a run of consecutive
 // ket pairs of one molecule) from a shared counter until the chunk list, ordered by
@@ -626,6 +688,11 @@ __global__ void __launch_bounds__(128) eri_queue_{tag}(const EriQueue Q) {{
         const int p = ch.x, cnt = ch.z & 0xffff, lg = (ch.z >> 16) & 7, lgj = (ch.z >> 20) & 7;
         const int W = 32 >> lg, kq = lane & (W - 1), s = lane >> (5 - lg);
         const int js = s & ((1 << lgj) - 1), is = s >> lgj;
+        double jab[JK ? {na * nb} : 1];  // J/K digestion: the bra pair's J, over the chunk
+        if constexpr (JK) {{
+#pragma unroll
+            for (int x = 0; x < {na * nb}; ++x) jab[x] = 0.0;
+        }}
         for (int base = 0; base < cnt; base += W) {{
         const int q = ch.y + base + kq;
         const bool live = base + kq < cnt;
@@ -655,12 +722,24 @@ __global__ void __launch_bounds__(128) eri_queue_{tag}(const EriQueue Q) {{
             double res[{nout}];
             hrr_{tag}(Q.pairs, p, q, acc, res);
             if constexpr (JK) {{
-                jk_{tag}(Q.jk, __ldg(&Q.pairs.info[p]), __ldg(&Q.pairs.info[q]), p == q, res);
+                const int4 ib_ = __ldg(&Q.pairs.info[p]), ik_ = __ldg(&Q.pairs.info[q]);
+                jk_{tag}(Q.jk, ib_, ik_, jk_weight(ib_.z == ib_.w, ik_.z == ik_.w, p == q), res, jab);
             }} else {{
                 store_{tag}(Q.out + __ldg(&Q.mol_out[ch.w]), __ldg(&Q.pairs.info[p]), __ldg(&Q.pairs.info[q]),
                             p == q, res);
             }}
         }}
+        }}
+        if constexpr (JK) {{
+            // one addition per J_ab and chunk
+            const int4 ib_ = __ldg(&Q.pairs.info[p]);
+#pragma unroll
+            for (int x = 0; x < {na * nb}; ++x) {{
+                double v = jab[x];
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+                if (lane == 0) atomicAdd(&Q.jk.J[(long long)(ib_.z + x / {nb}) * Q.jk.n + ib_.w + x % {nb}], 2.0 * v);
+            }}
         }}
     }}
 }}

@@ -12621,17 +12621,1572 @@ __device__ __forceinline__ void store_dddd(double *__restrict__ out, const int4 
       if ((!dab || 5 >= 5) && (!dcd || 5 >= 5) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[1295]; }
 }
 
-// The quartet's unique integrals digested into J and K (molints_plan_jk) instead of stored.
-__device__ __noinline__ void jk_dddd(const JKOut &jk, const int4 ib_, const int4 ik_, bool same,
-                                      const double *__restrict__ res) {
-    const bool dab = ib_.z == ib_.w, dcd = ik_.z == ik_.w;
-    for (int x = 0; x < 1296; ++x) {
-        const int ia = x / 216, ibb = (x / 36) % 6, ic = (x / 6) % 6, id = x % 6;
-        if ((dab && ia < ibb) || (dcd && ic < id)) continue;
-        const int i = ib_.z + ia, j = ib_.w + ibb, k = ik_.z + ic, l = ik_.w + id;
-        if (same && pair_index(i, j) < pair_index(k, l)) continue;
-        jk_add(jk, i, j, k, l, res[x]);
+// The quartet's share of J and K (molints_plan_jk, eri_common.cuh): every integral of the block,
+// times f, into one orientation of each target; J_ab stays in the lane (one bra pair per chunk).
+__device__ __forceinline__ void jk_dddd(const JKOut &jk, const int4 ib_, const int4 ik_, double f,
+                                         const double *__restrict__ res, double *__restrict__ jab) {
+    const long long n = jk.n;
+    const double *__restrict__ D = jk.D;
+    const double *__restrict__ Db = D + ib_.w * n, *__restrict__ Dc = D + ik_.z * n;
+    double dcd[36], dbc[36], dbd[36], jcd[36], kbc[36], kbd[36];
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+#pragma unroll
+        for (int l = 0; l < 6; ++l) {
+            dcd[k * 6 + l] = __ldg(&Dc[k * n + ik_.w + l]);
+            jcd[k * 6 + l] = 0.0;
+        }
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            dbc[j * 6 + k] = __ldg(&Db[j * n + ik_.z + k]);
+            kbc[j * 6 + k] = 0.0;
+        }
+#pragma unroll
+        for (int l = 0; l < 6; ++l) {
+            dbd[j * 6 + l] = __ldg(&Db[j * n + ik_.w + l]);
+            kbd[j * 6 + l] = 0.0;
+        }
     }
+#pragma unroll 1
+    for (int i = 0; i < 6; ++i) {
+        const double *__restrict__ Da = D + (ib_.z + i) * n;
+        double dab[6], dac[6], dad[6], kac[6], kad[6];
+#pragma unroll
+        for (int j = 0; j < 6; ++j) dab[j] = __ldg(&Da[ib_.w + j]);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) { dac[k] = __ldg(&Da[ik_.z + k]); kac[k] = 0.0; }
+#pragma unroll
+        for (int l = 0; l < 6; ++l) { dad[l] = __ldg(&Da[ik_.w + l]); kad[l] = 0.0; }
+        { const double v = f * res[(i * 6 + 0) * 36 + 0];
+          jab[i * 6 + 0] = fma(dcd[0], v, jab[i * 6 + 0]);
+          jcd[0] = fma(dab[0], v, jcd[0]);
+          kac[0] = fma(dbd[0], v, kac[0]);
+          kad[0] = fma(dbc[0], v, kad[0]);
+          kbc[0] = fma(dad[0], v, kbc[0]);
+          kbd[0] = fma(dac[0], v, kbd[0]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 1];
+          jab[i * 6 + 0] = fma(dcd[1], v, jab[i * 6 + 0]);
+          jcd[1] = fma(dab[0], v, jcd[1]);
+          kac[0] = fma(dbd[1], v, kac[0]);
+          kad[1] = fma(dbc[0], v, kad[1]);
+          kbc[0] = fma(dad[1], v, kbc[0]);
+          kbd[1] = fma(dac[0], v, kbd[1]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 2];
+          jab[i * 6 + 0] = fma(dcd[2], v, jab[i * 6 + 0]);
+          jcd[2] = fma(dab[0], v, jcd[2]);
+          kac[0] = fma(dbd[2], v, kac[0]);
+          kad[2] = fma(dbc[0], v, kad[2]);
+          kbc[0] = fma(dad[2], v, kbc[0]);
+          kbd[2] = fma(dac[0], v, kbd[2]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 3];
+          jab[i * 6 + 0] = fma(dcd[3], v, jab[i * 6 + 0]);
+          jcd[3] = fma(dab[0], v, jcd[3]);
+          kac[0] = fma(dbd[3], v, kac[0]);
+          kad[3] = fma(dbc[0], v, kad[3]);
+          kbc[0] = fma(dad[3], v, kbc[0]);
+          kbd[3] = fma(dac[0], v, kbd[3]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 4];
+          jab[i * 6 + 0] = fma(dcd[4], v, jab[i * 6 + 0]);
+          jcd[4] = fma(dab[0], v, jcd[4]);
+          kac[0] = fma(dbd[4], v, kac[0]);
+          kad[4] = fma(dbc[0], v, kad[4]);
+          kbc[0] = fma(dad[4], v, kbc[0]);
+          kbd[4] = fma(dac[0], v, kbd[4]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 5];
+          jab[i * 6 + 0] = fma(dcd[5], v, jab[i * 6 + 0]);
+          jcd[5] = fma(dab[0], v, jcd[5]);
+          kac[0] = fma(dbd[5], v, kac[0]);
+          kad[5] = fma(dbc[0], v, kad[5]);
+          kbc[0] = fma(dad[5], v, kbc[0]);
+          kbd[5] = fma(dac[0], v, kbd[5]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 6];
+          jab[i * 6 + 0] = fma(dcd[6], v, jab[i * 6 + 0]);
+          jcd[6] = fma(dab[0], v, jcd[6]);
+          kac[1] = fma(dbd[0], v, kac[1]);
+          kad[0] = fma(dbc[1], v, kad[0]);
+          kbc[1] = fma(dad[0], v, kbc[1]);
+          kbd[0] = fma(dac[1], v, kbd[0]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 7];
+          jab[i * 6 + 0] = fma(dcd[7], v, jab[i * 6 + 0]);
+          jcd[7] = fma(dab[0], v, jcd[7]);
+          kac[1] = fma(dbd[1], v, kac[1]);
+          kad[1] = fma(dbc[1], v, kad[1]);
+          kbc[1] = fma(dad[1], v, kbc[1]);
+          kbd[1] = fma(dac[1], v, kbd[1]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 8];
+          jab[i * 6 + 0] = fma(dcd[8], v, jab[i * 6 + 0]);
+          jcd[8] = fma(dab[0], v, jcd[8]);
+          kac[1] = fma(dbd[2], v, kac[1]);
+          kad[2] = fma(dbc[1], v, kad[2]);
+          kbc[1] = fma(dad[2], v, kbc[1]);
+          kbd[2] = fma(dac[1], v, kbd[2]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 9];
+          jab[i * 6 + 0] = fma(dcd[9], v, jab[i * 6 + 0]);
+          jcd[9] = fma(dab[0], v, jcd[9]);
+          kac[1] = fma(dbd[3], v, kac[1]);
+          kad[3] = fma(dbc[1], v, kad[3]);
+          kbc[1] = fma(dad[3], v, kbc[1]);
+          kbd[3] = fma(dac[1], v, kbd[3]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 10];
+          jab[i * 6 + 0] = fma(dcd[10], v, jab[i * 6 + 0]);
+          jcd[10] = fma(dab[0], v, jcd[10]);
+          kac[1] = fma(dbd[4], v, kac[1]);
+          kad[4] = fma(dbc[1], v, kad[4]);
+          kbc[1] = fma(dad[4], v, kbc[1]);
+          kbd[4] = fma(dac[1], v, kbd[4]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 11];
+          jab[i * 6 + 0] = fma(dcd[11], v, jab[i * 6 + 0]);
+          jcd[11] = fma(dab[0], v, jcd[11]);
+          kac[1] = fma(dbd[5], v, kac[1]);
+          kad[5] = fma(dbc[1], v, kad[5]);
+          kbc[1] = fma(dad[5], v, kbc[1]);
+          kbd[5] = fma(dac[1], v, kbd[5]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 12];
+          jab[i * 6 + 0] = fma(dcd[12], v, jab[i * 6 + 0]);
+          jcd[12] = fma(dab[0], v, jcd[12]);
+          kac[2] = fma(dbd[0], v, kac[2]);
+          kad[0] = fma(dbc[2], v, kad[0]);
+          kbc[2] = fma(dad[0], v, kbc[2]);
+          kbd[0] = fma(dac[2], v, kbd[0]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 13];
+          jab[i * 6 + 0] = fma(dcd[13], v, jab[i * 6 + 0]);
+          jcd[13] = fma(dab[0], v, jcd[13]);
+          kac[2] = fma(dbd[1], v, kac[2]);
+          kad[1] = fma(dbc[2], v, kad[1]);
+          kbc[2] = fma(dad[1], v, kbc[2]);
+          kbd[1] = fma(dac[2], v, kbd[1]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 14];
+          jab[i * 6 + 0] = fma(dcd[14], v, jab[i * 6 + 0]);
+          jcd[14] = fma(dab[0], v, jcd[14]);
+          kac[2] = fma(dbd[2], v, kac[2]);
+          kad[2] = fma(dbc[2], v, kad[2]);
+          kbc[2] = fma(dad[2], v, kbc[2]);
+          kbd[2] = fma(dac[2], v, kbd[2]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 15];
+          jab[i * 6 + 0] = fma(dcd[15], v, jab[i * 6 + 0]);
+          jcd[15] = fma(dab[0], v, jcd[15]);
+          kac[2] = fma(dbd[3], v, kac[2]);
+          kad[3] = fma(dbc[2], v, kad[3]);
+          kbc[2] = fma(dad[3], v, kbc[2]);
+          kbd[3] = fma(dac[2], v, kbd[3]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 16];
+          jab[i * 6 + 0] = fma(dcd[16], v, jab[i * 6 + 0]);
+          jcd[16] = fma(dab[0], v, jcd[16]);
+          kac[2] = fma(dbd[4], v, kac[2]);
+          kad[4] = fma(dbc[2], v, kad[4]);
+          kbc[2] = fma(dad[4], v, kbc[2]);
+          kbd[4] = fma(dac[2], v, kbd[4]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 17];
+          jab[i * 6 + 0] = fma(dcd[17], v, jab[i * 6 + 0]);
+          jcd[17] = fma(dab[0], v, jcd[17]);
+          kac[2] = fma(dbd[5], v, kac[2]);
+          kad[5] = fma(dbc[2], v, kad[5]);
+          kbc[2] = fma(dad[5], v, kbc[2]);
+          kbd[5] = fma(dac[2], v, kbd[5]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 18];
+          jab[i * 6 + 0] = fma(dcd[18], v, jab[i * 6 + 0]);
+          jcd[18] = fma(dab[0], v, jcd[18]);
+          kac[3] = fma(dbd[0], v, kac[3]);
+          kad[0] = fma(dbc[3], v, kad[0]);
+          kbc[3] = fma(dad[0], v, kbc[3]);
+          kbd[0] = fma(dac[3], v, kbd[0]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 19];
+          jab[i * 6 + 0] = fma(dcd[19], v, jab[i * 6 + 0]);
+          jcd[19] = fma(dab[0], v, jcd[19]);
+          kac[3] = fma(dbd[1], v, kac[3]);
+          kad[1] = fma(dbc[3], v, kad[1]);
+          kbc[3] = fma(dad[1], v, kbc[3]);
+          kbd[1] = fma(dac[3], v, kbd[1]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 20];
+          jab[i * 6 + 0] = fma(dcd[20], v, jab[i * 6 + 0]);
+          jcd[20] = fma(dab[0], v, jcd[20]);
+          kac[3] = fma(dbd[2], v, kac[3]);
+          kad[2] = fma(dbc[3], v, kad[2]);
+          kbc[3] = fma(dad[2], v, kbc[3]);
+          kbd[2] = fma(dac[3], v, kbd[2]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 21];
+          jab[i * 6 + 0] = fma(dcd[21], v, jab[i * 6 + 0]);
+          jcd[21] = fma(dab[0], v, jcd[21]);
+          kac[3] = fma(dbd[3], v, kac[3]);
+          kad[3] = fma(dbc[3], v, kad[3]);
+          kbc[3] = fma(dad[3], v, kbc[3]);
+          kbd[3] = fma(dac[3], v, kbd[3]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 22];
+          jab[i * 6 + 0] = fma(dcd[22], v, jab[i * 6 + 0]);
+          jcd[22] = fma(dab[0], v, jcd[22]);
+          kac[3] = fma(dbd[4], v, kac[3]);
+          kad[4] = fma(dbc[3], v, kad[4]);
+          kbc[3] = fma(dad[4], v, kbc[3]);
+          kbd[4] = fma(dac[3], v, kbd[4]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 23];
+          jab[i * 6 + 0] = fma(dcd[23], v, jab[i * 6 + 0]);
+          jcd[23] = fma(dab[0], v, jcd[23]);
+          kac[3] = fma(dbd[5], v, kac[3]);
+          kad[5] = fma(dbc[3], v, kad[5]);
+          kbc[3] = fma(dad[5], v, kbc[3]);
+          kbd[5] = fma(dac[3], v, kbd[5]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 24];
+          jab[i * 6 + 0] = fma(dcd[24], v, jab[i * 6 + 0]);
+          jcd[24] = fma(dab[0], v, jcd[24]);
+          kac[4] = fma(dbd[0], v, kac[4]);
+          kad[0] = fma(dbc[4], v, kad[0]);
+          kbc[4] = fma(dad[0], v, kbc[4]);
+          kbd[0] = fma(dac[4], v, kbd[0]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 25];
+          jab[i * 6 + 0] = fma(dcd[25], v, jab[i * 6 + 0]);
+          jcd[25] = fma(dab[0], v, jcd[25]);
+          kac[4] = fma(dbd[1], v, kac[4]);
+          kad[1] = fma(dbc[4], v, kad[1]);
+          kbc[4] = fma(dad[1], v, kbc[4]);
+          kbd[1] = fma(dac[4], v, kbd[1]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 26];
+          jab[i * 6 + 0] = fma(dcd[26], v, jab[i * 6 + 0]);
+          jcd[26] = fma(dab[0], v, jcd[26]);
+          kac[4] = fma(dbd[2], v, kac[4]);
+          kad[2] = fma(dbc[4], v, kad[2]);
+          kbc[4] = fma(dad[2], v, kbc[4]);
+          kbd[2] = fma(dac[4], v, kbd[2]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 27];
+          jab[i * 6 + 0] = fma(dcd[27], v, jab[i * 6 + 0]);
+          jcd[27] = fma(dab[0], v, jcd[27]);
+          kac[4] = fma(dbd[3], v, kac[4]);
+          kad[3] = fma(dbc[4], v, kad[3]);
+          kbc[4] = fma(dad[3], v, kbc[4]);
+          kbd[3] = fma(dac[4], v, kbd[3]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 28];
+          jab[i * 6 + 0] = fma(dcd[28], v, jab[i * 6 + 0]);
+          jcd[28] = fma(dab[0], v, jcd[28]);
+          kac[4] = fma(dbd[4], v, kac[4]);
+          kad[4] = fma(dbc[4], v, kad[4]);
+          kbc[4] = fma(dad[4], v, kbc[4]);
+          kbd[4] = fma(dac[4], v, kbd[4]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 29];
+          jab[i * 6 + 0] = fma(dcd[29], v, jab[i * 6 + 0]);
+          jcd[29] = fma(dab[0], v, jcd[29]);
+          kac[4] = fma(dbd[5], v, kac[4]);
+          kad[5] = fma(dbc[4], v, kad[5]);
+          kbc[4] = fma(dad[5], v, kbc[4]);
+          kbd[5] = fma(dac[4], v, kbd[5]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 30];
+          jab[i * 6 + 0] = fma(dcd[30], v, jab[i * 6 + 0]);
+          jcd[30] = fma(dab[0], v, jcd[30]);
+          kac[5] = fma(dbd[0], v, kac[5]);
+          kad[0] = fma(dbc[5], v, kad[0]);
+          kbc[5] = fma(dad[0], v, kbc[5]);
+          kbd[0] = fma(dac[5], v, kbd[0]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 31];
+          jab[i * 6 + 0] = fma(dcd[31], v, jab[i * 6 + 0]);
+          jcd[31] = fma(dab[0], v, jcd[31]);
+          kac[5] = fma(dbd[1], v, kac[5]);
+          kad[1] = fma(dbc[5], v, kad[1]);
+          kbc[5] = fma(dad[1], v, kbc[5]);
+          kbd[1] = fma(dac[5], v, kbd[1]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 32];
+          jab[i * 6 + 0] = fma(dcd[32], v, jab[i * 6 + 0]);
+          jcd[32] = fma(dab[0], v, jcd[32]);
+          kac[5] = fma(dbd[2], v, kac[5]);
+          kad[2] = fma(dbc[5], v, kad[2]);
+          kbc[5] = fma(dad[2], v, kbc[5]);
+          kbd[2] = fma(dac[5], v, kbd[2]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 33];
+          jab[i * 6 + 0] = fma(dcd[33], v, jab[i * 6 + 0]);
+          jcd[33] = fma(dab[0], v, jcd[33]);
+          kac[5] = fma(dbd[3], v, kac[5]);
+          kad[3] = fma(dbc[5], v, kad[3]);
+          kbc[5] = fma(dad[3], v, kbc[5]);
+          kbd[3] = fma(dac[5], v, kbd[3]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 34];
+          jab[i * 6 + 0] = fma(dcd[34], v, jab[i * 6 + 0]);
+          jcd[34] = fma(dab[0], v, jcd[34]);
+          kac[5] = fma(dbd[4], v, kac[5]);
+          kad[4] = fma(dbc[5], v, kad[4]);
+          kbc[5] = fma(dad[4], v, kbc[5]);
+          kbd[4] = fma(dac[5], v, kbd[4]); }
+        { const double v = f * res[(i * 6 + 0) * 36 + 35];
+          jab[i * 6 + 0] = fma(dcd[35], v, jab[i * 6 + 0]);
+          jcd[35] = fma(dab[0], v, jcd[35]);
+          kac[5] = fma(dbd[5], v, kac[5]);
+          kad[5] = fma(dbc[5], v, kad[5]);
+          kbc[5] = fma(dad[5], v, kbc[5]);
+          kbd[5] = fma(dac[5], v, kbd[5]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 0];
+          jab[i * 6 + 1] = fma(dcd[0], v, jab[i * 6 + 1]);
+          jcd[0] = fma(dab[1], v, jcd[0]);
+          kac[0] = fma(dbd[6], v, kac[0]);
+          kad[0] = fma(dbc[6], v, kad[0]);
+          kbc[6] = fma(dad[0], v, kbc[6]);
+          kbd[6] = fma(dac[0], v, kbd[6]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 1];
+          jab[i * 6 + 1] = fma(dcd[1], v, jab[i * 6 + 1]);
+          jcd[1] = fma(dab[1], v, jcd[1]);
+          kac[0] = fma(dbd[7], v, kac[0]);
+          kad[1] = fma(dbc[6], v, kad[1]);
+          kbc[6] = fma(dad[1], v, kbc[6]);
+          kbd[7] = fma(dac[0], v, kbd[7]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 2];
+          jab[i * 6 + 1] = fma(dcd[2], v, jab[i * 6 + 1]);
+          jcd[2] = fma(dab[1], v, jcd[2]);
+          kac[0] = fma(dbd[8], v, kac[0]);
+          kad[2] = fma(dbc[6], v, kad[2]);
+          kbc[6] = fma(dad[2], v, kbc[6]);
+          kbd[8] = fma(dac[0], v, kbd[8]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 3];
+          jab[i * 6 + 1] = fma(dcd[3], v, jab[i * 6 + 1]);
+          jcd[3] = fma(dab[1], v, jcd[3]);
+          kac[0] = fma(dbd[9], v, kac[0]);
+          kad[3] = fma(dbc[6], v, kad[3]);
+          kbc[6] = fma(dad[3], v, kbc[6]);
+          kbd[9] = fma(dac[0], v, kbd[9]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 4];
+          jab[i * 6 + 1] = fma(dcd[4], v, jab[i * 6 + 1]);
+          jcd[4] = fma(dab[1], v, jcd[4]);
+          kac[0] = fma(dbd[10], v, kac[0]);
+          kad[4] = fma(dbc[6], v, kad[4]);
+          kbc[6] = fma(dad[4], v, kbc[6]);
+          kbd[10] = fma(dac[0], v, kbd[10]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 5];
+          jab[i * 6 + 1] = fma(dcd[5], v, jab[i * 6 + 1]);
+          jcd[5] = fma(dab[1], v, jcd[5]);
+          kac[0] = fma(dbd[11], v, kac[0]);
+          kad[5] = fma(dbc[6], v, kad[5]);
+          kbc[6] = fma(dad[5], v, kbc[6]);
+          kbd[11] = fma(dac[0], v, kbd[11]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 6];
+          jab[i * 6 + 1] = fma(dcd[6], v, jab[i * 6 + 1]);
+          jcd[6] = fma(dab[1], v, jcd[6]);
+          kac[1] = fma(dbd[6], v, kac[1]);
+          kad[0] = fma(dbc[7], v, kad[0]);
+          kbc[7] = fma(dad[0], v, kbc[7]);
+          kbd[6] = fma(dac[1], v, kbd[6]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 7];
+          jab[i * 6 + 1] = fma(dcd[7], v, jab[i * 6 + 1]);
+          jcd[7] = fma(dab[1], v, jcd[7]);
+          kac[1] = fma(dbd[7], v, kac[1]);
+          kad[1] = fma(dbc[7], v, kad[1]);
+          kbc[7] = fma(dad[1], v, kbc[7]);
+          kbd[7] = fma(dac[1], v, kbd[7]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 8];
+          jab[i * 6 + 1] = fma(dcd[8], v, jab[i * 6 + 1]);
+          jcd[8] = fma(dab[1], v, jcd[8]);
+          kac[1] = fma(dbd[8], v, kac[1]);
+          kad[2] = fma(dbc[7], v, kad[2]);
+          kbc[7] = fma(dad[2], v, kbc[7]);
+          kbd[8] = fma(dac[1], v, kbd[8]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 9];
+          jab[i * 6 + 1] = fma(dcd[9], v, jab[i * 6 + 1]);
+          jcd[9] = fma(dab[1], v, jcd[9]);
+          kac[1] = fma(dbd[9], v, kac[1]);
+          kad[3] = fma(dbc[7], v, kad[3]);
+          kbc[7] = fma(dad[3], v, kbc[7]);
+          kbd[9] = fma(dac[1], v, kbd[9]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 10];
+          jab[i * 6 + 1] = fma(dcd[10], v, jab[i * 6 + 1]);
+          jcd[10] = fma(dab[1], v, jcd[10]);
+          kac[1] = fma(dbd[10], v, kac[1]);
+          kad[4] = fma(dbc[7], v, kad[4]);
+          kbc[7] = fma(dad[4], v, kbc[7]);
+          kbd[10] = fma(dac[1], v, kbd[10]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 11];
+          jab[i * 6 + 1] = fma(dcd[11], v, jab[i * 6 + 1]);
+          jcd[11] = fma(dab[1], v, jcd[11]);
+          kac[1] = fma(dbd[11], v, kac[1]);
+          kad[5] = fma(dbc[7], v, kad[5]);
+          kbc[7] = fma(dad[5], v, kbc[7]);
+          kbd[11] = fma(dac[1], v, kbd[11]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 12];
+          jab[i * 6 + 1] = fma(dcd[12], v, jab[i * 6 + 1]);
+          jcd[12] = fma(dab[1], v, jcd[12]);
+          kac[2] = fma(dbd[6], v, kac[2]);
+          kad[0] = fma(dbc[8], v, kad[0]);
+          kbc[8] = fma(dad[0], v, kbc[8]);
+          kbd[6] = fma(dac[2], v, kbd[6]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 13];
+          jab[i * 6 + 1] = fma(dcd[13], v, jab[i * 6 + 1]);
+          jcd[13] = fma(dab[1], v, jcd[13]);
+          kac[2] = fma(dbd[7], v, kac[2]);
+          kad[1] = fma(dbc[8], v, kad[1]);
+          kbc[8] = fma(dad[1], v, kbc[8]);
+          kbd[7] = fma(dac[2], v, kbd[7]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 14];
+          jab[i * 6 + 1] = fma(dcd[14], v, jab[i * 6 + 1]);
+          jcd[14] = fma(dab[1], v, jcd[14]);
+          kac[2] = fma(dbd[8], v, kac[2]);
+          kad[2] = fma(dbc[8], v, kad[2]);
+          kbc[8] = fma(dad[2], v, kbc[8]);
+          kbd[8] = fma(dac[2], v, kbd[8]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 15];
+          jab[i * 6 + 1] = fma(dcd[15], v, jab[i * 6 + 1]);
+          jcd[15] = fma(dab[1], v, jcd[15]);
+          kac[2] = fma(dbd[9], v, kac[2]);
+          kad[3] = fma(dbc[8], v, kad[3]);
+          kbc[8] = fma(dad[3], v, kbc[8]);
+          kbd[9] = fma(dac[2], v, kbd[9]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 16];
+          jab[i * 6 + 1] = fma(dcd[16], v, jab[i * 6 + 1]);
+          jcd[16] = fma(dab[1], v, jcd[16]);
+          kac[2] = fma(dbd[10], v, kac[2]);
+          kad[4] = fma(dbc[8], v, kad[4]);
+          kbc[8] = fma(dad[4], v, kbc[8]);
+          kbd[10] = fma(dac[2], v, kbd[10]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 17];
+          jab[i * 6 + 1] = fma(dcd[17], v, jab[i * 6 + 1]);
+          jcd[17] = fma(dab[1], v, jcd[17]);
+          kac[2] = fma(dbd[11], v, kac[2]);
+          kad[5] = fma(dbc[8], v, kad[5]);
+          kbc[8] = fma(dad[5], v, kbc[8]);
+          kbd[11] = fma(dac[2], v, kbd[11]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 18];
+          jab[i * 6 + 1] = fma(dcd[18], v, jab[i * 6 + 1]);
+          jcd[18] = fma(dab[1], v, jcd[18]);
+          kac[3] = fma(dbd[6], v, kac[3]);
+          kad[0] = fma(dbc[9], v, kad[0]);
+          kbc[9] = fma(dad[0], v, kbc[9]);
+          kbd[6] = fma(dac[3], v, kbd[6]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 19];
+          jab[i * 6 + 1] = fma(dcd[19], v, jab[i * 6 + 1]);
+          jcd[19] = fma(dab[1], v, jcd[19]);
+          kac[3] = fma(dbd[7], v, kac[3]);
+          kad[1] = fma(dbc[9], v, kad[1]);
+          kbc[9] = fma(dad[1], v, kbc[9]);
+          kbd[7] = fma(dac[3], v, kbd[7]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 20];
+          jab[i * 6 + 1] = fma(dcd[20], v, jab[i * 6 + 1]);
+          jcd[20] = fma(dab[1], v, jcd[20]);
+          kac[3] = fma(dbd[8], v, kac[3]);
+          kad[2] = fma(dbc[9], v, kad[2]);
+          kbc[9] = fma(dad[2], v, kbc[9]);
+          kbd[8] = fma(dac[3], v, kbd[8]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 21];
+          jab[i * 6 + 1] = fma(dcd[21], v, jab[i * 6 + 1]);
+          jcd[21] = fma(dab[1], v, jcd[21]);
+          kac[3] = fma(dbd[9], v, kac[3]);
+          kad[3] = fma(dbc[9], v, kad[3]);
+          kbc[9] = fma(dad[3], v, kbc[9]);
+          kbd[9] = fma(dac[3], v, kbd[9]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 22];
+          jab[i * 6 + 1] = fma(dcd[22], v, jab[i * 6 + 1]);
+          jcd[22] = fma(dab[1], v, jcd[22]);
+          kac[3] = fma(dbd[10], v, kac[3]);
+          kad[4] = fma(dbc[9], v, kad[4]);
+          kbc[9] = fma(dad[4], v, kbc[9]);
+          kbd[10] = fma(dac[3], v, kbd[10]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 23];
+          jab[i * 6 + 1] = fma(dcd[23], v, jab[i * 6 + 1]);
+          jcd[23] = fma(dab[1], v, jcd[23]);
+          kac[3] = fma(dbd[11], v, kac[3]);
+          kad[5] = fma(dbc[9], v, kad[5]);
+          kbc[9] = fma(dad[5], v, kbc[9]);
+          kbd[11] = fma(dac[3], v, kbd[11]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 24];
+          jab[i * 6 + 1] = fma(dcd[24], v, jab[i * 6 + 1]);
+          jcd[24] = fma(dab[1], v, jcd[24]);
+          kac[4] = fma(dbd[6], v, kac[4]);
+          kad[0] = fma(dbc[10], v, kad[0]);
+          kbc[10] = fma(dad[0], v, kbc[10]);
+          kbd[6] = fma(dac[4], v, kbd[6]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 25];
+          jab[i * 6 + 1] = fma(dcd[25], v, jab[i * 6 + 1]);
+          jcd[25] = fma(dab[1], v, jcd[25]);
+          kac[4] = fma(dbd[7], v, kac[4]);
+          kad[1] = fma(dbc[10], v, kad[1]);
+          kbc[10] = fma(dad[1], v, kbc[10]);
+          kbd[7] = fma(dac[4], v, kbd[7]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 26];
+          jab[i * 6 + 1] = fma(dcd[26], v, jab[i * 6 + 1]);
+          jcd[26] = fma(dab[1], v, jcd[26]);
+          kac[4] = fma(dbd[8], v, kac[4]);
+          kad[2] = fma(dbc[10], v, kad[2]);
+          kbc[10] = fma(dad[2], v, kbc[10]);
+          kbd[8] = fma(dac[4], v, kbd[8]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 27];
+          jab[i * 6 + 1] = fma(dcd[27], v, jab[i * 6 + 1]);
+          jcd[27] = fma(dab[1], v, jcd[27]);
+          kac[4] = fma(dbd[9], v, kac[4]);
+          kad[3] = fma(dbc[10], v, kad[3]);
+          kbc[10] = fma(dad[3], v, kbc[10]);
+          kbd[9] = fma(dac[4], v, kbd[9]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 28];
+          jab[i * 6 + 1] = fma(dcd[28], v, jab[i * 6 + 1]);
+          jcd[28] = fma(dab[1], v, jcd[28]);
+          kac[4] = fma(dbd[10], v, kac[4]);
+          kad[4] = fma(dbc[10], v, kad[4]);
+          kbc[10] = fma(dad[4], v, kbc[10]);
+          kbd[10] = fma(dac[4], v, kbd[10]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 29];
+          jab[i * 6 + 1] = fma(dcd[29], v, jab[i * 6 + 1]);
+          jcd[29] = fma(dab[1], v, jcd[29]);
+          kac[4] = fma(dbd[11], v, kac[4]);
+          kad[5] = fma(dbc[10], v, kad[5]);
+          kbc[10] = fma(dad[5], v, kbc[10]);
+          kbd[11] = fma(dac[4], v, kbd[11]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 30];
+          jab[i * 6 + 1] = fma(dcd[30], v, jab[i * 6 + 1]);
+          jcd[30] = fma(dab[1], v, jcd[30]);
+          kac[5] = fma(dbd[6], v, kac[5]);
+          kad[0] = fma(dbc[11], v, kad[0]);
+          kbc[11] = fma(dad[0], v, kbc[11]);
+          kbd[6] = fma(dac[5], v, kbd[6]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 31];
+          jab[i * 6 + 1] = fma(dcd[31], v, jab[i * 6 + 1]);
+          jcd[31] = fma(dab[1], v, jcd[31]);
+          kac[5] = fma(dbd[7], v, kac[5]);
+          kad[1] = fma(dbc[11], v, kad[1]);
+          kbc[11] = fma(dad[1], v, kbc[11]);
+          kbd[7] = fma(dac[5], v, kbd[7]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 32];
+          jab[i * 6 + 1] = fma(dcd[32], v, jab[i * 6 + 1]);
+          jcd[32] = fma(dab[1], v, jcd[32]);
+          kac[5] = fma(dbd[8], v, kac[5]);
+          kad[2] = fma(dbc[11], v, kad[2]);
+          kbc[11] = fma(dad[2], v, kbc[11]);
+          kbd[8] = fma(dac[5], v, kbd[8]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 33];
+          jab[i * 6 + 1] = fma(dcd[33], v, jab[i * 6 + 1]);
+          jcd[33] = fma(dab[1], v, jcd[33]);
+          kac[5] = fma(dbd[9], v, kac[5]);
+          kad[3] = fma(dbc[11], v, kad[3]);
+          kbc[11] = fma(dad[3], v, kbc[11]);
+          kbd[9] = fma(dac[5], v, kbd[9]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 34];
+          jab[i * 6 + 1] = fma(dcd[34], v, jab[i * 6 + 1]);
+          jcd[34] = fma(dab[1], v, jcd[34]);
+          kac[5] = fma(dbd[10], v, kac[5]);
+          kad[4] = fma(dbc[11], v, kad[4]);
+          kbc[11] = fma(dad[4], v, kbc[11]);
+          kbd[10] = fma(dac[5], v, kbd[10]); }
+        { const double v = f * res[(i * 6 + 1) * 36 + 35];
+          jab[i * 6 + 1] = fma(dcd[35], v, jab[i * 6 + 1]);
+          jcd[35] = fma(dab[1], v, jcd[35]);
+          kac[5] = fma(dbd[11], v, kac[5]);
+          kad[5] = fma(dbc[11], v, kad[5]);
+          kbc[11] = fma(dad[5], v, kbc[11]);
+          kbd[11] = fma(dac[5], v, kbd[11]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 0];
+          jab[i * 6 + 2] = fma(dcd[0], v, jab[i * 6 + 2]);
+          jcd[0] = fma(dab[2], v, jcd[0]);
+          kac[0] = fma(dbd[12], v, kac[0]);
+          kad[0] = fma(dbc[12], v, kad[0]);
+          kbc[12] = fma(dad[0], v, kbc[12]);
+          kbd[12] = fma(dac[0], v, kbd[12]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 1];
+          jab[i * 6 + 2] = fma(dcd[1], v, jab[i * 6 + 2]);
+          jcd[1] = fma(dab[2], v, jcd[1]);
+          kac[0] = fma(dbd[13], v, kac[0]);
+          kad[1] = fma(dbc[12], v, kad[1]);
+          kbc[12] = fma(dad[1], v, kbc[12]);
+          kbd[13] = fma(dac[0], v, kbd[13]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 2];
+          jab[i * 6 + 2] = fma(dcd[2], v, jab[i * 6 + 2]);
+          jcd[2] = fma(dab[2], v, jcd[2]);
+          kac[0] = fma(dbd[14], v, kac[0]);
+          kad[2] = fma(dbc[12], v, kad[2]);
+          kbc[12] = fma(dad[2], v, kbc[12]);
+          kbd[14] = fma(dac[0], v, kbd[14]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 3];
+          jab[i * 6 + 2] = fma(dcd[3], v, jab[i * 6 + 2]);
+          jcd[3] = fma(dab[2], v, jcd[3]);
+          kac[0] = fma(dbd[15], v, kac[0]);
+          kad[3] = fma(dbc[12], v, kad[3]);
+          kbc[12] = fma(dad[3], v, kbc[12]);
+          kbd[15] = fma(dac[0], v, kbd[15]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 4];
+          jab[i * 6 + 2] = fma(dcd[4], v, jab[i * 6 + 2]);
+          jcd[4] = fma(dab[2], v, jcd[4]);
+          kac[0] = fma(dbd[16], v, kac[0]);
+          kad[4] = fma(dbc[12], v, kad[4]);
+          kbc[12] = fma(dad[4], v, kbc[12]);
+          kbd[16] = fma(dac[0], v, kbd[16]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 5];
+          jab[i * 6 + 2] = fma(dcd[5], v, jab[i * 6 + 2]);
+          jcd[5] = fma(dab[2], v, jcd[5]);
+          kac[0] = fma(dbd[17], v, kac[0]);
+          kad[5] = fma(dbc[12], v, kad[5]);
+          kbc[12] = fma(dad[5], v, kbc[12]);
+          kbd[17] = fma(dac[0], v, kbd[17]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 6];
+          jab[i * 6 + 2] = fma(dcd[6], v, jab[i * 6 + 2]);
+          jcd[6] = fma(dab[2], v, jcd[6]);
+          kac[1] = fma(dbd[12], v, kac[1]);
+          kad[0] = fma(dbc[13], v, kad[0]);
+          kbc[13] = fma(dad[0], v, kbc[13]);
+          kbd[12] = fma(dac[1], v, kbd[12]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 7];
+          jab[i * 6 + 2] = fma(dcd[7], v, jab[i * 6 + 2]);
+          jcd[7] = fma(dab[2], v, jcd[7]);
+          kac[1] = fma(dbd[13], v, kac[1]);
+          kad[1] = fma(dbc[13], v, kad[1]);
+          kbc[13] = fma(dad[1], v, kbc[13]);
+          kbd[13] = fma(dac[1], v, kbd[13]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 8];
+          jab[i * 6 + 2] = fma(dcd[8], v, jab[i * 6 + 2]);
+          jcd[8] = fma(dab[2], v, jcd[8]);
+          kac[1] = fma(dbd[14], v, kac[1]);
+          kad[2] = fma(dbc[13], v, kad[2]);
+          kbc[13] = fma(dad[2], v, kbc[13]);
+          kbd[14] = fma(dac[1], v, kbd[14]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 9];
+          jab[i * 6 + 2] = fma(dcd[9], v, jab[i * 6 + 2]);
+          jcd[9] = fma(dab[2], v, jcd[9]);
+          kac[1] = fma(dbd[15], v, kac[1]);
+          kad[3] = fma(dbc[13], v, kad[3]);
+          kbc[13] = fma(dad[3], v, kbc[13]);
+          kbd[15] = fma(dac[1], v, kbd[15]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 10];
+          jab[i * 6 + 2] = fma(dcd[10], v, jab[i * 6 + 2]);
+          jcd[10] = fma(dab[2], v, jcd[10]);
+          kac[1] = fma(dbd[16], v, kac[1]);
+          kad[4] = fma(dbc[13], v, kad[4]);
+          kbc[13] = fma(dad[4], v, kbc[13]);
+          kbd[16] = fma(dac[1], v, kbd[16]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 11];
+          jab[i * 6 + 2] = fma(dcd[11], v, jab[i * 6 + 2]);
+          jcd[11] = fma(dab[2], v, jcd[11]);
+          kac[1] = fma(dbd[17], v, kac[1]);
+          kad[5] = fma(dbc[13], v, kad[5]);
+          kbc[13] = fma(dad[5], v, kbc[13]);
+          kbd[17] = fma(dac[1], v, kbd[17]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 12];
+          jab[i * 6 + 2] = fma(dcd[12], v, jab[i * 6 + 2]);
+          jcd[12] = fma(dab[2], v, jcd[12]);
+          kac[2] = fma(dbd[12], v, kac[2]);
+          kad[0] = fma(dbc[14], v, kad[0]);
+          kbc[14] = fma(dad[0], v, kbc[14]);
+          kbd[12] = fma(dac[2], v, kbd[12]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 13];
+          jab[i * 6 + 2] = fma(dcd[13], v, jab[i * 6 + 2]);
+          jcd[13] = fma(dab[2], v, jcd[13]);
+          kac[2] = fma(dbd[13], v, kac[2]);
+          kad[1] = fma(dbc[14], v, kad[1]);
+          kbc[14] = fma(dad[1], v, kbc[14]);
+          kbd[13] = fma(dac[2], v, kbd[13]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 14];
+          jab[i * 6 + 2] = fma(dcd[14], v, jab[i * 6 + 2]);
+          jcd[14] = fma(dab[2], v, jcd[14]);
+          kac[2] = fma(dbd[14], v, kac[2]);
+          kad[2] = fma(dbc[14], v, kad[2]);
+          kbc[14] = fma(dad[2], v, kbc[14]);
+          kbd[14] = fma(dac[2], v, kbd[14]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 15];
+          jab[i * 6 + 2] = fma(dcd[15], v, jab[i * 6 + 2]);
+          jcd[15] = fma(dab[2], v, jcd[15]);
+          kac[2] = fma(dbd[15], v, kac[2]);
+          kad[3] = fma(dbc[14], v, kad[3]);
+          kbc[14] = fma(dad[3], v, kbc[14]);
+          kbd[15] = fma(dac[2], v, kbd[15]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 16];
+          jab[i * 6 + 2] = fma(dcd[16], v, jab[i * 6 + 2]);
+          jcd[16] = fma(dab[2], v, jcd[16]);
+          kac[2] = fma(dbd[16], v, kac[2]);
+          kad[4] = fma(dbc[14], v, kad[4]);
+          kbc[14] = fma(dad[4], v, kbc[14]);
+          kbd[16] = fma(dac[2], v, kbd[16]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 17];
+          jab[i * 6 + 2] = fma(dcd[17], v, jab[i * 6 + 2]);
+          jcd[17] = fma(dab[2], v, jcd[17]);
+          kac[2] = fma(dbd[17], v, kac[2]);
+          kad[5] = fma(dbc[14], v, kad[5]);
+          kbc[14] = fma(dad[5], v, kbc[14]);
+          kbd[17] = fma(dac[2], v, kbd[17]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 18];
+          jab[i * 6 + 2] = fma(dcd[18], v, jab[i * 6 + 2]);
+          jcd[18] = fma(dab[2], v, jcd[18]);
+          kac[3] = fma(dbd[12], v, kac[3]);
+          kad[0] = fma(dbc[15], v, kad[0]);
+          kbc[15] = fma(dad[0], v, kbc[15]);
+          kbd[12] = fma(dac[3], v, kbd[12]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 19];
+          jab[i * 6 + 2] = fma(dcd[19], v, jab[i * 6 + 2]);
+          jcd[19] = fma(dab[2], v, jcd[19]);
+          kac[3] = fma(dbd[13], v, kac[3]);
+          kad[1] = fma(dbc[15], v, kad[1]);
+          kbc[15] = fma(dad[1], v, kbc[15]);
+          kbd[13] = fma(dac[3], v, kbd[13]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 20];
+          jab[i * 6 + 2] = fma(dcd[20], v, jab[i * 6 + 2]);
+          jcd[20] = fma(dab[2], v, jcd[20]);
+          kac[3] = fma(dbd[14], v, kac[3]);
+          kad[2] = fma(dbc[15], v, kad[2]);
+          kbc[15] = fma(dad[2], v, kbc[15]);
+          kbd[14] = fma(dac[3], v, kbd[14]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 21];
+          jab[i * 6 + 2] = fma(dcd[21], v, jab[i * 6 + 2]);
+          jcd[21] = fma(dab[2], v, jcd[21]);
+          kac[3] = fma(dbd[15], v, kac[3]);
+          kad[3] = fma(dbc[15], v, kad[3]);
+          kbc[15] = fma(dad[3], v, kbc[15]);
+          kbd[15] = fma(dac[3], v, kbd[15]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 22];
+          jab[i * 6 + 2] = fma(dcd[22], v, jab[i * 6 + 2]);
+          jcd[22] = fma(dab[2], v, jcd[22]);
+          kac[3] = fma(dbd[16], v, kac[3]);
+          kad[4] = fma(dbc[15], v, kad[4]);
+          kbc[15] = fma(dad[4], v, kbc[15]);
+          kbd[16] = fma(dac[3], v, kbd[16]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 23];
+          jab[i * 6 + 2] = fma(dcd[23], v, jab[i * 6 + 2]);
+          jcd[23] = fma(dab[2], v, jcd[23]);
+          kac[3] = fma(dbd[17], v, kac[3]);
+          kad[5] = fma(dbc[15], v, kad[5]);
+          kbc[15] = fma(dad[5], v, kbc[15]);
+          kbd[17] = fma(dac[3], v, kbd[17]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 24];
+          jab[i * 6 + 2] = fma(dcd[24], v, jab[i * 6 + 2]);
+          jcd[24] = fma(dab[2], v, jcd[24]);
+          kac[4] = fma(dbd[12], v, kac[4]);
+          kad[0] = fma(dbc[16], v, kad[0]);
+          kbc[16] = fma(dad[0], v, kbc[16]);
+          kbd[12] = fma(dac[4], v, kbd[12]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 25];
+          jab[i * 6 + 2] = fma(dcd[25], v, jab[i * 6 + 2]);
+          jcd[25] = fma(dab[2], v, jcd[25]);
+          kac[4] = fma(dbd[13], v, kac[4]);
+          kad[1] = fma(dbc[16], v, kad[1]);
+          kbc[16] = fma(dad[1], v, kbc[16]);
+          kbd[13] = fma(dac[4], v, kbd[13]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 26];
+          jab[i * 6 + 2] = fma(dcd[26], v, jab[i * 6 + 2]);
+          jcd[26] = fma(dab[2], v, jcd[26]);
+          kac[4] = fma(dbd[14], v, kac[4]);
+          kad[2] = fma(dbc[16], v, kad[2]);
+          kbc[16] = fma(dad[2], v, kbc[16]);
+          kbd[14] = fma(dac[4], v, kbd[14]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 27];
+          jab[i * 6 + 2] = fma(dcd[27], v, jab[i * 6 + 2]);
+          jcd[27] = fma(dab[2], v, jcd[27]);
+          kac[4] = fma(dbd[15], v, kac[4]);
+          kad[3] = fma(dbc[16], v, kad[3]);
+          kbc[16] = fma(dad[3], v, kbc[16]);
+          kbd[15] = fma(dac[4], v, kbd[15]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 28];
+          jab[i * 6 + 2] = fma(dcd[28], v, jab[i * 6 + 2]);
+          jcd[28] = fma(dab[2], v, jcd[28]);
+          kac[4] = fma(dbd[16], v, kac[4]);
+          kad[4] = fma(dbc[16], v, kad[4]);
+          kbc[16] = fma(dad[4], v, kbc[16]);
+          kbd[16] = fma(dac[4], v, kbd[16]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 29];
+          jab[i * 6 + 2] = fma(dcd[29], v, jab[i * 6 + 2]);
+          jcd[29] = fma(dab[2], v, jcd[29]);
+          kac[4] = fma(dbd[17], v, kac[4]);
+          kad[5] = fma(dbc[16], v, kad[5]);
+          kbc[16] = fma(dad[5], v, kbc[16]);
+          kbd[17] = fma(dac[4], v, kbd[17]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 30];
+          jab[i * 6 + 2] = fma(dcd[30], v, jab[i * 6 + 2]);
+          jcd[30] = fma(dab[2], v, jcd[30]);
+          kac[5] = fma(dbd[12], v, kac[5]);
+          kad[0] = fma(dbc[17], v, kad[0]);
+          kbc[17] = fma(dad[0], v, kbc[17]);
+          kbd[12] = fma(dac[5], v, kbd[12]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 31];
+          jab[i * 6 + 2] = fma(dcd[31], v, jab[i * 6 + 2]);
+          jcd[31] = fma(dab[2], v, jcd[31]);
+          kac[5] = fma(dbd[13], v, kac[5]);
+          kad[1] = fma(dbc[17], v, kad[1]);
+          kbc[17] = fma(dad[1], v, kbc[17]);
+          kbd[13] = fma(dac[5], v, kbd[13]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 32];
+          jab[i * 6 + 2] = fma(dcd[32], v, jab[i * 6 + 2]);
+          jcd[32] = fma(dab[2], v, jcd[32]);
+          kac[5] = fma(dbd[14], v, kac[5]);
+          kad[2] = fma(dbc[17], v, kad[2]);
+          kbc[17] = fma(dad[2], v, kbc[17]);
+          kbd[14] = fma(dac[5], v, kbd[14]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 33];
+          jab[i * 6 + 2] = fma(dcd[33], v, jab[i * 6 + 2]);
+          jcd[33] = fma(dab[2], v, jcd[33]);
+          kac[5] = fma(dbd[15], v, kac[5]);
+          kad[3] = fma(dbc[17], v, kad[3]);
+          kbc[17] = fma(dad[3], v, kbc[17]);
+          kbd[15] = fma(dac[5], v, kbd[15]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 34];
+          jab[i * 6 + 2] = fma(dcd[34], v, jab[i * 6 + 2]);
+          jcd[34] = fma(dab[2], v, jcd[34]);
+          kac[5] = fma(dbd[16], v, kac[5]);
+          kad[4] = fma(dbc[17], v, kad[4]);
+          kbc[17] = fma(dad[4], v, kbc[17]);
+          kbd[16] = fma(dac[5], v, kbd[16]); }
+        { const double v = f * res[(i * 6 + 2) * 36 + 35];
+          jab[i * 6 + 2] = fma(dcd[35], v, jab[i * 6 + 2]);
+          jcd[35] = fma(dab[2], v, jcd[35]);
+          kac[5] = fma(dbd[17], v, kac[5]);
+          kad[5] = fma(dbc[17], v, kad[5]);
+          kbc[17] = fma(dad[5], v, kbc[17]);
+          kbd[17] = fma(dac[5], v, kbd[17]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 0];
+          jab[i * 6 + 3] = fma(dcd[0], v, jab[i * 6 + 3]);
+          jcd[0] = fma(dab[3], v, jcd[0]);
+          kac[0] = fma(dbd[18], v, kac[0]);
+          kad[0] = fma(dbc[18], v, kad[0]);
+          kbc[18] = fma(dad[0], v, kbc[18]);
+          kbd[18] = fma(dac[0], v, kbd[18]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 1];
+          jab[i * 6 + 3] = fma(dcd[1], v, jab[i * 6 + 3]);
+          jcd[1] = fma(dab[3], v, jcd[1]);
+          kac[0] = fma(dbd[19], v, kac[0]);
+          kad[1] = fma(dbc[18], v, kad[1]);
+          kbc[18] = fma(dad[1], v, kbc[18]);
+          kbd[19] = fma(dac[0], v, kbd[19]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 2];
+          jab[i * 6 + 3] = fma(dcd[2], v, jab[i * 6 + 3]);
+          jcd[2] = fma(dab[3], v, jcd[2]);
+          kac[0] = fma(dbd[20], v, kac[0]);
+          kad[2] = fma(dbc[18], v, kad[2]);
+          kbc[18] = fma(dad[2], v, kbc[18]);
+          kbd[20] = fma(dac[0], v, kbd[20]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 3];
+          jab[i * 6 + 3] = fma(dcd[3], v, jab[i * 6 + 3]);
+          jcd[3] = fma(dab[3], v, jcd[3]);
+          kac[0] = fma(dbd[21], v, kac[0]);
+          kad[3] = fma(dbc[18], v, kad[3]);
+          kbc[18] = fma(dad[3], v, kbc[18]);
+          kbd[21] = fma(dac[0], v, kbd[21]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 4];
+          jab[i * 6 + 3] = fma(dcd[4], v, jab[i * 6 + 3]);
+          jcd[4] = fma(dab[3], v, jcd[4]);
+          kac[0] = fma(dbd[22], v, kac[0]);
+          kad[4] = fma(dbc[18], v, kad[4]);
+          kbc[18] = fma(dad[4], v, kbc[18]);
+          kbd[22] = fma(dac[0], v, kbd[22]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 5];
+          jab[i * 6 + 3] = fma(dcd[5], v, jab[i * 6 + 3]);
+          jcd[5] = fma(dab[3], v, jcd[5]);
+          kac[0] = fma(dbd[23], v, kac[0]);
+          kad[5] = fma(dbc[18], v, kad[5]);
+          kbc[18] = fma(dad[5], v, kbc[18]);
+          kbd[23] = fma(dac[0], v, kbd[23]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 6];
+          jab[i * 6 + 3] = fma(dcd[6], v, jab[i * 6 + 3]);
+          jcd[6] = fma(dab[3], v, jcd[6]);
+          kac[1] = fma(dbd[18], v, kac[1]);
+          kad[0] = fma(dbc[19], v, kad[0]);
+          kbc[19] = fma(dad[0], v, kbc[19]);
+          kbd[18] = fma(dac[1], v, kbd[18]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 7];
+          jab[i * 6 + 3] = fma(dcd[7], v, jab[i * 6 + 3]);
+          jcd[7] = fma(dab[3], v, jcd[7]);
+          kac[1] = fma(dbd[19], v, kac[1]);
+          kad[1] = fma(dbc[19], v, kad[1]);
+          kbc[19] = fma(dad[1], v, kbc[19]);
+          kbd[19] = fma(dac[1], v, kbd[19]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 8];
+          jab[i * 6 + 3] = fma(dcd[8], v, jab[i * 6 + 3]);
+          jcd[8] = fma(dab[3], v, jcd[8]);
+          kac[1] = fma(dbd[20], v, kac[1]);
+          kad[2] = fma(dbc[19], v, kad[2]);
+          kbc[19] = fma(dad[2], v, kbc[19]);
+          kbd[20] = fma(dac[1], v, kbd[20]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 9];
+          jab[i * 6 + 3] = fma(dcd[9], v, jab[i * 6 + 3]);
+          jcd[9] = fma(dab[3], v, jcd[9]);
+          kac[1] = fma(dbd[21], v, kac[1]);
+          kad[3] = fma(dbc[19], v, kad[3]);
+          kbc[19] = fma(dad[3], v, kbc[19]);
+          kbd[21] = fma(dac[1], v, kbd[21]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 10];
+          jab[i * 6 + 3] = fma(dcd[10], v, jab[i * 6 + 3]);
+          jcd[10] = fma(dab[3], v, jcd[10]);
+          kac[1] = fma(dbd[22], v, kac[1]);
+          kad[4] = fma(dbc[19], v, kad[4]);
+          kbc[19] = fma(dad[4], v, kbc[19]);
+          kbd[22] = fma(dac[1], v, kbd[22]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 11];
+          jab[i * 6 + 3] = fma(dcd[11], v, jab[i * 6 + 3]);
+          jcd[11] = fma(dab[3], v, jcd[11]);
+          kac[1] = fma(dbd[23], v, kac[1]);
+          kad[5] = fma(dbc[19], v, kad[5]);
+          kbc[19] = fma(dad[5], v, kbc[19]);
+          kbd[23] = fma(dac[1], v, kbd[23]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 12];
+          jab[i * 6 + 3] = fma(dcd[12], v, jab[i * 6 + 3]);
+          jcd[12] = fma(dab[3], v, jcd[12]);
+          kac[2] = fma(dbd[18], v, kac[2]);
+          kad[0] = fma(dbc[20], v, kad[0]);
+          kbc[20] = fma(dad[0], v, kbc[20]);
+          kbd[18] = fma(dac[2], v, kbd[18]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 13];
+          jab[i * 6 + 3] = fma(dcd[13], v, jab[i * 6 + 3]);
+          jcd[13] = fma(dab[3], v, jcd[13]);
+          kac[2] = fma(dbd[19], v, kac[2]);
+          kad[1] = fma(dbc[20], v, kad[1]);
+          kbc[20] = fma(dad[1], v, kbc[20]);
+          kbd[19] = fma(dac[2], v, kbd[19]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 14];
+          jab[i * 6 + 3] = fma(dcd[14], v, jab[i * 6 + 3]);
+          jcd[14] = fma(dab[3], v, jcd[14]);
+          kac[2] = fma(dbd[20], v, kac[2]);
+          kad[2] = fma(dbc[20], v, kad[2]);
+          kbc[20] = fma(dad[2], v, kbc[20]);
+          kbd[20] = fma(dac[2], v, kbd[20]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 15];
+          jab[i * 6 + 3] = fma(dcd[15], v, jab[i * 6 + 3]);
+          jcd[15] = fma(dab[3], v, jcd[15]);
+          kac[2] = fma(dbd[21], v, kac[2]);
+          kad[3] = fma(dbc[20], v, kad[3]);
+          kbc[20] = fma(dad[3], v, kbc[20]);
+          kbd[21] = fma(dac[2], v, kbd[21]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 16];
+          jab[i * 6 + 3] = fma(dcd[16], v, jab[i * 6 + 3]);
+          jcd[16] = fma(dab[3], v, jcd[16]);
+          kac[2] = fma(dbd[22], v, kac[2]);
+          kad[4] = fma(dbc[20], v, kad[4]);
+          kbc[20] = fma(dad[4], v, kbc[20]);
+          kbd[22] = fma(dac[2], v, kbd[22]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 17];
+          jab[i * 6 + 3] = fma(dcd[17], v, jab[i * 6 + 3]);
+          jcd[17] = fma(dab[3], v, jcd[17]);
+          kac[2] = fma(dbd[23], v, kac[2]);
+          kad[5] = fma(dbc[20], v, kad[5]);
+          kbc[20] = fma(dad[5], v, kbc[20]);
+          kbd[23] = fma(dac[2], v, kbd[23]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 18];
+          jab[i * 6 + 3] = fma(dcd[18], v, jab[i * 6 + 3]);
+          jcd[18] = fma(dab[3], v, jcd[18]);
+          kac[3] = fma(dbd[18], v, kac[3]);
+          kad[0] = fma(dbc[21], v, kad[0]);
+          kbc[21] = fma(dad[0], v, kbc[21]);
+          kbd[18] = fma(dac[3], v, kbd[18]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 19];
+          jab[i * 6 + 3] = fma(dcd[19], v, jab[i * 6 + 3]);
+          jcd[19] = fma(dab[3], v, jcd[19]);
+          kac[3] = fma(dbd[19], v, kac[3]);
+          kad[1] = fma(dbc[21], v, kad[1]);
+          kbc[21] = fma(dad[1], v, kbc[21]);
+          kbd[19] = fma(dac[3], v, kbd[19]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 20];
+          jab[i * 6 + 3] = fma(dcd[20], v, jab[i * 6 + 3]);
+          jcd[20] = fma(dab[3], v, jcd[20]);
+          kac[3] = fma(dbd[20], v, kac[3]);
+          kad[2] = fma(dbc[21], v, kad[2]);
+          kbc[21] = fma(dad[2], v, kbc[21]);
+          kbd[20] = fma(dac[3], v, kbd[20]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 21];
+          jab[i * 6 + 3] = fma(dcd[21], v, jab[i * 6 + 3]);
+          jcd[21] = fma(dab[3], v, jcd[21]);
+          kac[3] = fma(dbd[21], v, kac[3]);
+          kad[3] = fma(dbc[21], v, kad[3]);
+          kbc[21] = fma(dad[3], v, kbc[21]);
+          kbd[21] = fma(dac[3], v, kbd[21]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 22];
+          jab[i * 6 + 3] = fma(dcd[22], v, jab[i * 6 + 3]);
+          jcd[22] = fma(dab[3], v, jcd[22]);
+          kac[3] = fma(dbd[22], v, kac[3]);
+          kad[4] = fma(dbc[21], v, kad[4]);
+          kbc[21] = fma(dad[4], v, kbc[21]);
+          kbd[22] = fma(dac[3], v, kbd[22]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 23];
+          jab[i * 6 + 3] = fma(dcd[23], v, jab[i * 6 + 3]);
+          jcd[23] = fma(dab[3], v, jcd[23]);
+          kac[3] = fma(dbd[23], v, kac[3]);
+          kad[5] = fma(dbc[21], v, kad[5]);
+          kbc[21] = fma(dad[5], v, kbc[21]);
+          kbd[23] = fma(dac[3], v, kbd[23]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 24];
+          jab[i * 6 + 3] = fma(dcd[24], v, jab[i * 6 + 3]);
+          jcd[24] = fma(dab[3], v, jcd[24]);
+          kac[4] = fma(dbd[18], v, kac[4]);
+          kad[0] = fma(dbc[22], v, kad[0]);
+          kbc[22] = fma(dad[0], v, kbc[22]);
+          kbd[18] = fma(dac[4], v, kbd[18]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 25];
+          jab[i * 6 + 3] = fma(dcd[25], v, jab[i * 6 + 3]);
+          jcd[25] = fma(dab[3], v, jcd[25]);
+          kac[4] = fma(dbd[19], v, kac[4]);
+          kad[1] = fma(dbc[22], v, kad[1]);
+          kbc[22] = fma(dad[1], v, kbc[22]);
+          kbd[19] = fma(dac[4], v, kbd[19]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 26];
+          jab[i * 6 + 3] = fma(dcd[26], v, jab[i * 6 + 3]);
+          jcd[26] = fma(dab[3], v, jcd[26]);
+          kac[4] = fma(dbd[20], v, kac[4]);
+          kad[2] = fma(dbc[22], v, kad[2]);
+          kbc[22] = fma(dad[2], v, kbc[22]);
+          kbd[20] = fma(dac[4], v, kbd[20]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 27];
+          jab[i * 6 + 3] = fma(dcd[27], v, jab[i * 6 + 3]);
+          jcd[27] = fma(dab[3], v, jcd[27]);
+          kac[4] = fma(dbd[21], v, kac[4]);
+          kad[3] = fma(dbc[22], v, kad[3]);
+          kbc[22] = fma(dad[3], v, kbc[22]);
+          kbd[21] = fma(dac[4], v, kbd[21]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 28];
+          jab[i * 6 + 3] = fma(dcd[28], v, jab[i * 6 + 3]);
+          jcd[28] = fma(dab[3], v, jcd[28]);
+          kac[4] = fma(dbd[22], v, kac[4]);
+          kad[4] = fma(dbc[22], v, kad[4]);
+          kbc[22] = fma(dad[4], v, kbc[22]);
+          kbd[22] = fma(dac[4], v, kbd[22]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 29];
+          jab[i * 6 + 3] = fma(dcd[29], v, jab[i * 6 + 3]);
+          jcd[29] = fma(dab[3], v, jcd[29]);
+          kac[4] = fma(dbd[23], v, kac[4]);
+          kad[5] = fma(dbc[22], v, kad[5]);
+          kbc[22] = fma(dad[5], v, kbc[22]);
+          kbd[23] = fma(dac[4], v, kbd[23]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 30];
+          jab[i * 6 + 3] = fma(dcd[30], v, jab[i * 6 + 3]);
+          jcd[30] = fma(dab[3], v, jcd[30]);
+          kac[5] = fma(dbd[18], v, kac[5]);
+          kad[0] = fma(dbc[23], v, kad[0]);
+          kbc[23] = fma(dad[0], v, kbc[23]);
+          kbd[18] = fma(dac[5], v, kbd[18]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 31];
+          jab[i * 6 + 3] = fma(dcd[31], v, jab[i * 6 + 3]);
+          jcd[31] = fma(dab[3], v, jcd[31]);
+          kac[5] = fma(dbd[19], v, kac[5]);
+          kad[1] = fma(dbc[23], v, kad[1]);
+          kbc[23] = fma(dad[1], v, kbc[23]);
+          kbd[19] = fma(dac[5], v, kbd[19]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 32];
+          jab[i * 6 + 3] = fma(dcd[32], v, jab[i * 6 + 3]);
+          jcd[32] = fma(dab[3], v, jcd[32]);
+          kac[5] = fma(dbd[20], v, kac[5]);
+          kad[2] = fma(dbc[23], v, kad[2]);
+          kbc[23] = fma(dad[2], v, kbc[23]);
+          kbd[20] = fma(dac[5], v, kbd[20]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 33];
+          jab[i * 6 + 3] = fma(dcd[33], v, jab[i * 6 + 3]);
+          jcd[33] = fma(dab[3], v, jcd[33]);
+          kac[5] = fma(dbd[21], v, kac[5]);
+          kad[3] = fma(dbc[23], v, kad[3]);
+          kbc[23] = fma(dad[3], v, kbc[23]);
+          kbd[21] = fma(dac[5], v, kbd[21]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 34];
+          jab[i * 6 + 3] = fma(dcd[34], v, jab[i * 6 + 3]);
+          jcd[34] = fma(dab[3], v, jcd[34]);
+          kac[5] = fma(dbd[22], v, kac[5]);
+          kad[4] = fma(dbc[23], v, kad[4]);
+          kbc[23] = fma(dad[4], v, kbc[23]);
+          kbd[22] = fma(dac[5], v, kbd[22]); }
+        { const double v = f * res[(i * 6 + 3) * 36 + 35];
+          jab[i * 6 + 3] = fma(dcd[35], v, jab[i * 6 + 3]);
+          jcd[35] = fma(dab[3], v, jcd[35]);
+          kac[5] = fma(dbd[23], v, kac[5]);
+          kad[5] = fma(dbc[23], v, kad[5]);
+          kbc[23] = fma(dad[5], v, kbc[23]);
+          kbd[23] = fma(dac[5], v, kbd[23]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 0];
+          jab[i * 6 + 4] = fma(dcd[0], v, jab[i * 6 + 4]);
+          jcd[0] = fma(dab[4], v, jcd[0]);
+          kac[0] = fma(dbd[24], v, kac[0]);
+          kad[0] = fma(dbc[24], v, kad[0]);
+          kbc[24] = fma(dad[0], v, kbc[24]);
+          kbd[24] = fma(dac[0], v, kbd[24]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 1];
+          jab[i * 6 + 4] = fma(dcd[1], v, jab[i * 6 + 4]);
+          jcd[1] = fma(dab[4], v, jcd[1]);
+          kac[0] = fma(dbd[25], v, kac[0]);
+          kad[1] = fma(dbc[24], v, kad[1]);
+          kbc[24] = fma(dad[1], v, kbc[24]);
+          kbd[25] = fma(dac[0], v, kbd[25]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 2];
+          jab[i * 6 + 4] = fma(dcd[2], v, jab[i * 6 + 4]);
+          jcd[2] = fma(dab[4], v, jcd[2]);
+          kac[0] = fma(dbd[26], v, kac[0]);
+          kad[2] = fma(dbc[24], v, kad[2]);
+          kbc[24] = fma(dad[2], v, kbc[24]);
+          kbd[26] = fma(dac[0], v, kbd[26]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 3];
+          jab[i * 6 + 4] = fma(dcd[3], v, jab[i * 6 + 4]);
+          jcd[3] = fma(dab[4], v, jcd[3]);
+          kac[0] = fma(dbd[27], v, kac[0]);
+          kad[3] = fma(dbc[24], v, kad[3]);
+          kbc[24] = fma(dad[3], v, kbc[24]);
+          kbd[27] = fma(dac[0], v, kbd[27]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 4];
+          jab[i * 6 + 4] = fma(dcd[4], v, jab[i * 6 + 4]);
+          jcd[4] = fma(dab[4], v, jcd[4]);
+          kac[0] = fma(dbd[28], v, kac[0]);
+          kad[4] = fma(dbc[24], v, kad[4]);
+          kbc[24] = fma(dad[4], v, kbc[24]);
+          kbd[28] = fma(dac[0], v, kbd[28]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 5];
+          jab[i * 6 + 4] = fma(dcd[5], v, jab[i * 6 + 4]);
+          jcd[5] = fma(dab[4], v, jcd[5]);
+          kac[0] = fma(dbd[29], v, kac[0]);
+          kad[5] = fma(dbc[24], v, kad[5]);
+          kbc[24] = fma(dad[5], v, kbc[24]);
+          kbd[29] = fma(dac[0], v, kbd[29]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 6];
+          jab[i * 6 + 4] = fma(dcd[6], v, jab[i * 6 + 4]);
+          jcd[6] = fma(dab[4], v, jcd[6]);
+          kac[1] = fma(dbd[24], v, kac[1]);
+          kad[0] = fma(dbc[25], v, kad[0]);
+          kbc[25] = fma(dad[0], v, kbc[25]);
+          kbd[24] = fma(dac[1], v, kbd[24]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 7];
+          jab[i * 6 + 4] = fma(dcd[7], v, jab[i * 6 + 4]);
+          jcd[7] = fma(dab[4], v, jcd[7]);
+          kac[1] = fma(dbd[25], v, kac[1]);
+          kad[1] = fma(dbc[25], v, kad[1]);
+          kbc[25] = fma(dad[1], v, kbc[25]);
+          kbd[25] = fma(dac[1], v, kbd[25]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 8];
+          jab[i * 6 + 4] = fma(dcd[8], v, jab[i * 6 + 4]);
+          jcd[8] = fma(dab[4], v, jcd[8]);
+          kac[1] = fma(dbd[26], v, kac[1]);
+          kad[2] = fma(dbc[25], v, kad[2]);
+          kbc[25] = fma(dad[2], v, kbc[25]);
+          kbd[26] = fma(dac[1], v, kbd[26]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 9];
+          jab[i * 6 + 4] = fma(dcd[9], v, jab[i * 6 + 4]);
+          jcd[9] = fma(dab[4], v, jcd[9]);
+          kac[1] = fma(dbd[27], v, kac[1]);
+          kad[3] = fma(dbc[25], v, kad[3]);
+          kbc[25] = fma(dad[3], v, kbc[25]);
+          kbd[27] = fma(dac[1], v, kbd[27]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 10];
+          jab[i * 6 + 4] = fma(dcd[10], v, jab[i * 6 + 4]);
+          jcd[10] = fma(dab[4], v, jcd[10]);
+          kac[1] = fma(dbd[28], v, kac[1]);
+          kad[4] = fma(dbc[25], v, kad[4]);
+          kbc[25] = fma(dad[4], v, kbc[25]);
+          kbd[28] = fma(dac[1], v, kbd[28]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 11];
+          jab[i * 6 + 4] = fma(dcd[11], v, jab[i * 6 + 4]);
+          jcd[11] = fma(dab[4], v, jcd[11]);
+          kac[1] = fma(dbd[29], v, kac[1]);
+          kad[5] = fma(dbc[25], v, kad[5]);
+          kbc[25] = fma(dad[5], v, kbc[25]);
+          kbd[29] = fma(dac[1], v, kbd[29]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 12];
+          jab[i * 6 + 4] = fma(dcd[12], v, jab[i * 6 + 4]);
+          jcd[12] = fma(dab[4], v, jcd[12]);
+          kac[2] = fma(dbd[24], v, kac[2]);
+          kad[0] = fma(dbc[26], v, kad[0]);
+          kbc[26] = fma(dad[0], v, kbc[26]);
+          kbd[24] = fma(dac[2], v, kbd[24]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 13];
+          jab[i * 6 + 4] = fma(dcd[13], v, jab[i * 6 + 4]);
+          jcd[13] = fma(dab[4], v, jcd[13]);
+          kac[2] = fma(dbd[25], v, kac[2]);
+          kad[1] = fma(dbc[26], v, kad[1]);
+          kbc[26] = fma(dad[1], v, kbc[26]);
+          kbd[25] = fma(dac[2], v, kbd[25]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 14];
+          jab[i * 6 + 4] = fma(dcd[14], v, jab[i * 6 + 4]);
+          jcd[14] = fma(dab[4], v, jcd[14]);
+          kac[2] = fma(dbd[26], v, kac[2]);
+          kad[2] = fma(dbc[26], v, kad[2]);
+          kbc[26] = fma(dad[2], v, kbc[26]);
+          kbd[26] = fma(dac[2], v, kbd[26]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 15];
+          jab[i * 6 + 4] = fma(dcd[15], v, jab[i * 6 + 4]);
+          jcd[15] = fma(dab[4], v, jcd[15]);
+          kac[2] = fma(dbd[27], v, kac[2]);
+          kad[3] = fma(dbc[26], v, kad[3]);
+          kbc[26] = fma(dad[3], v, kbc[26]);
+          kbd[27] = fma(dac[2], v, kbd[27]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 16];
+          jab[i * 6 + 4] = fma(dcd[16], v, jab[i * 6 + 4]);
+          jcd[16] = fma(dab[4], v, jcd[16]);
+          kac[2] = fma(dbd[28], v, kac[2]);
+          kad[4] = fma(dbc[26], v, kad[4]);
+          kbc[26] = fma(dad[4], v, kbc[26]);
+          kbd[28] = fma(dac[2], v, kbd[28]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 17];
+          jab[i * 6 + 4] = fma(dcd[17], v, jab[i * 6 + 4]);
+          jcd[17] = fma(dab[4], v, jcd[17]);
+          kac[2] = fma(dbd[29], v, kac[2]);
+          kad[5] = fma(dbc[26], v, kad[5]);
+          kbc[26] = fma(dad[5], v, kbc[26]);
+          kbd[29] = fma(dac[2], v, kbd[29]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 18];
+          jab[i * 6 + 4] = fma(dcd[18], v, jab[i * 6 + 4]);
+          jcd[18] = fma(dab[4], v, jcd[18]);
+          kac[3] = fma(dbd[24], v, kac[3]);
+          kad[0] = fma(dbc[27], v, kad[0]);
+          kbc[27] = fma(dad[0], v, kbc[27]);
+          kbd[24] = fma(dac[3], v, kbd[24]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 19];
+          jab[i * 6 + 4] = fma(dcd[19], v, jab[i * 6 + 4]);
+          jcd[19] = fma(dab[4], v, jcd[19]);
+          kac[3] = fma(dbd[25], v, kac[3]);
+          kad[1] = fma(dbc[27], v, kad[1]);
+          kbc[27] = fma(dad[1], v, kbc[27]);
+          kbd[25] = fma(dac[3], v, kbd[25]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 20];
+          jab[i * 6 + 4] = fma(dcd[20], v, jab[i * 6 + 4]);
+          jcd[20] = fma(dab[4], v, jcd[20]);
+          kac[3] = fma(dbd[26], v, kac[3]);
+          kad[2] = fma(dbc[27], v, kad[2]);
+          kbc[27] = fma(dad[2], v, kbc[27]);
+          kbd[26] = fma(dac[3], v, kbd[26]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 21];
+          jab[i * 6 + 4] = fma(dcd[21], v, jab[i * 6 + 4]);
+          jcd[21] = fma(dab[4], v, jcd[21]);
+          kac[3] = fma(dbd[27], v, kac[3]);
+          kad[3] = fma(dbc[27], v, kad[3]);
+          kbc[27] = fma(dad[3], v, kbc[27]);
+          kbd[27] = fma(dac[3], v, kbd[27]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 22];
+          jab[i * 6 + 4] = fma(dcd[22], v, jab[i * 6 + 4]);
+          jcd[22] = fma(dab[4], v, jcd[22]);
+          kac[3] = fma(dbd[28], v, kac[3]);
+          kad[4] = fma(dbc[27], v, kad[4]);
+          kbc[27] = fma(dad[4], v, kbc[27]);
+          kbd[28] = fma(dac[3], v, kbd[28]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 23];
+          jab[i * 6 + 4] = fma(dcd[23], v, jab[i * 6 + 4]);
+          jcd[23] = fma(dab[4], v, jcd[23]);
+          kac[3] = fma(dbd[29], v, kac[3]);
+          kad[5] = fma(dbc[27], v, kad[5]);
+          kbc[27] = fma(dad[5], v, kbc[27]);
+          kbd[29] = fma(dac[3], v, kbd[29]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 24];
+          jab[i * 6 + 4] = fma(dcd[24], v, jab[i * 6 + 4]);
+          jcd[24] = fma(dab[4], v, jcd[24]);
+          kac[4] = fma(dbd[24], v, kac[4]);
+          kad[0] = fma(dbc[28], v, kad[0]);
+          kbc[28] = fma(dad[0], v, kbc[28]);
+          kbd[24] = fma(dac[4], v, kbd[24]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 25];
+          jab[i * 6 + 4] = fma(dcd[25], v, jab[i * 6 + 4]);
+          jcd[25] = fma(dab[4], v, jcd[25]);
+          kac[4] = fma(dbd[25], v, kac[4]);
+          kad[1] = fma(dbc[28], v, kad[1]);
+          kbc[28] = fma(dad[1], v, kbc[28]);
+          kbd[25] = fma(dac[4], v, kbd[25]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 26];
+          jab[i * 6 + 4] = fma(dcd[26], v, jab[i * 6 + 4]);
+          jcd[26] = fma(dab[4], v, jcd[26]);
+          kac[4] = fma(dbd[26], v, kac[4]);
+          kad[2] = fma(dbc[28], v, kad[2]);
+          kbc[28] = fma(dad[2], v, kbc[28]);
+          kbd[26] = fma(dac[4], v, kbd[26]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 27];
+          jab[i * 6 + 4] = fma(dcd[27], v, jab[i * 6 + 4]);
+          jcd[27] = fma(dab[4], v, jcd[27]);
+          kac[4] = fma(dbd[27], v, kac[4]);
+          kad[3] = fma(dbc[28], v, kad[3]);
+          kbc[28] = fma(dad[3], v, kbc[28]);
+          kbd[27] = fma(dac[4], v, kbd[27]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 28];
+          jab[i * 6 + 4] = fma(dcd[28], v, jab[i * 6 + 4]);
+          jcd[28] = fma(dab[4], v, jcd[28]);
+          kac[4] = fma(dbd[28], v, kac[4]);
+          kad[4] = fma(dbc[28], v, kad[4]);
+          kbc[28] = fma(dad[4], v, kbc[28]);
+          kbd[28] = fma(dac[4], v, kbd[28]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 29];
+          jab[i * 6 + 4] = fma(dcd[29], v, jab[i * 6 + 4]);
+          jcd[29] = fma(dab[4], v, jcd[29]);
+          kac[4] = fma(dbd[29], v, kac[4]);
+          kad[5] = fma(dbc[28], v, kad[5]);
+          kbc[28] = fma(dad[5], v, kbc[28]);
+          kbd[29] = fma(dac[4], v, kbd[29]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 30];
+          jab[i * 6 + 4] = fma(dcd[30], v, jab[i * 6 + 4]);
+          jcd[30] = fma(dab[4], v, jcd[30]);
+          kac[5] = fma(dbd[24], v, kac[5]);
+          kad[0] = fma(dbc[29], v, kad[0]);
+          kbc[29] = fma(dad[0], v, kbc[29]);
+          kbd[24] = fma(dac[5], v, kbd[24]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 31];
+          jab[i * 6 + 4] = fma(dcd[31], v, jab[i * 6 + 4]);
+          jcd[31] = fma(dab[4], v, jcd[31]);
+          kac[5] = fma(dbd[25], v, kac[5]);
+          kad[1] = fma(dbc[29], v, kad[1]);
+          kbc[29] = fma(dad[1], v, kbc[29]);
+          kbd[25] = fma(dac[5], v, kbd[25]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 32];
+          jab[i * 6 + 4] = fma(dcd[32], v, jab[i * 6 + 4]);
+          jcd[32] = fma(dab[4], v, jcd[32]);
+          kac[5] = fma(dbd[26], v, kac[5]);
+          kad[2] = fma(dbc[29], v, kad[2]);
+          kbc[29] = fma(dad[2], v, kbc[29]);
+          kbd[26] = fma(dac[5], v, kbd[26]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 33];
+          jab[i * 6 + 4] = fma(dcd[33], v, jab[i * 6 + 4]);
+          jcd[33] = fma(dab[4], v, jcd[33]);
+          kac[5] = fma(dbd[27], v, kac[5]);
+          kad[3] = fma(dbc[29], v, kad[3]);
+          kbc[29] = fma(dad[3], v, kbc[29]);
+          kbd[27] = fma(dac[5], v, kbd[27]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 34];
+          jab[i * 6 + 4] = fma(dcd[34], v, jab[i * 6 + 4]);
+          jcd[34] = fma(dab[4], v, jcd[34]);
+          kac[5] = fma(dbd[28], v, kac[5]);
+          kad[4] = fma(dbc[29], v, kad[4]);
+          kbc[29] = fma(dad[4], v, kbc[29]);
+          kbd[28] = fma(dac[5], v, kbd[28]); }
+        { const double v = f * res[(i * 6 + 4) * 36 + 35];
+          jab[i * 6 + 4] = fma(dcd[35], v, jab[i * 6 + 4]);
+          jcd[35] = fma(dab[4], v, jcd[35]);
+          kac[5] = fma(dbd[29], v, kac[5]);
+          kad[5] = fma(dbc[29], v, kad[5]);
+          kbc[29] = fma(dad[5], v, kbc[29]);
+          kbd[29] = fma(dac[5], v, kbd[29]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 0];
+          jab[i * 6 + 5] = fma(dcd[0], v, jab[i * 6 + 5]);
+          jcd[0] = fma(dab[5], v, jcd[0]);
+          kac[0] = fma(dbd[30], v, kac[0]);
+          kad[0] = fma(dbc[30], v, kad[0]);
+          kbc[30] = fma(dad[0], v, kbc[30]);
+          kbd[30] = fma(dac[0], v, kbd[30]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 1];
+          jab[i * 6 + 5] = fma(dcd[1], v, jab[i * 6 + 5]);
+          jcd[1] = fma(dab[5], v, jcd[1]);
+          kac[0] = fma(dbd[31], v, kac[0]);
+          kad[1] = fma(dbc[30], v, kad[1]);
+          kbc[30] = fma(dad[1], v, kbc[30]);
+          kbd[31] = fma(dac[0], v, kbd[31]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 2];
+          jab[i * 6 + 5] = fma(dcd[2], v, jab[i * 6 + 5]);
+          jcd[2] = fma(dab[5], v, jcd[2]);
+          kac[0] = fma(dbd[32], v, kac[0]);
+          kad[2] = fma(dbc[30], v, kad[2]);
+          kbc[30] = fma(dad[2], v, kbc[30]);
+          kbd[32] = fma(dac[0], v, kbd[32]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 3];
+          jab[i * 6 + 5] = fma(dcd[3], v, jab[i * 6 + 5]);
+          jcd[3] = fma(dab[5], v, jcd[3]);
+          kac[0] = fma(dbd[33], v, kac[0]);
+          kad[3] = fma(dbc[30], v, kad[3]);
+          kbc[30] = fma(dad[3], v, kbc[30]);
+          kbd[33] = fma(dac[0], v, kbd[33]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 4];
+          jab[i * 6 + 5] = fma(dcd[4], v, jab[i * 6 + 5]);
+          jcd[4] = fma(dab[5], v, jcd[4]);
+          kac[0] = fma(dbd[34], v, kac[0]);
+          kad[4] = fma(dbc[30], v, kad[4]);
+          kbc[30] = fma(dad[4], v, kbc[30]);
+          kbd[34] = fma(dac[0], v, kbd[34]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 5];
+          jab[i * 6 + 5] = fma(dcd[5], v, jab[i * 6 + 5]);
+          jcd[5] = fma(dab[5], v, jcd[5]);
+          kac[0] = fma(dbd[35], v, kac[0]);
+          kad[5] = fma(dbc[30], v, kad[5]);
+          kbc[30] = fma(dad[5], v, kbc[30]);
+          kbd[35] = fma(dac[0], v, kbd[35]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 6];
+          jab[i * 6 + 5] = fma(dcd[6], v, jab[i * 6 + 5]);
+          jcd[6] = fma(dab[5], v, jcd[6]);
+          kac[1] = fma(dbd[30], v, kac[1]);
+          kad[0] = fma(dbc[31], v, kad[0]);
+          kbc[31] = fma(dad[0], v, kbc[31]);
+          kbd[30] = fma(dac[1], v, kbd[30]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 7];
+          jab[i * 6 + 5] = fma(dcd[7], v, jab[i * 6 + 5]);
+          jcd[7] = fma(dab[5], v, jcd[7]);
+          kac[1] = fma(dbd[31], v, kac[1]);
+          kad[1] = fma(dbc[31], v, kad[1]);
+          kbc[31] = fma(dad[1], v, kbc[31]);
+          kbd[31] = fma(dac[1], v, kbd[31]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 8];
+          jab[i * 6 + 5] = fma(dcd[8], v, jab[i * 6 + 5]);
+          jcd[8] = fma(dab[5], v, jcd[8]);
+          kac[1] = fma(dbd[32], v, kac[1]);
+          kad[2] = fma(dbc[31], v, kad[2]);
+          kbc[31] = fma(dad[2], v, kbc[31]);
+          kbd[32] = fma(dac[1], v, kbd[32]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 9];
+          jab[i * 6 + 5] = fma(dcd[9], v, jab[i * 6 + 5]);
+          jcd[9] = fma(dab[5], v, jcd[9]);
+          kac[1] = fma(dbd[33], v, kac[1]);
+          kad[3] = fma(dbc[31], v, kad[3]);
+          kbc[31] = fma(dad[3], v, kbc[31]);
+          kbd[33] = fma(dac[1], v, kbd[33]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 10];
+          jab[i * 6 + 5] = fma(dcd[10], v, jab[i * 6 + 5]);
+          jcd[10] = fma(dab[5], v, jcd[10]);
+          kac[1] = fma(dbd[34], v, kac[1]);
+          kad[4] = fma(dbc[31], v, kad[4]);
+          kbc[31] = fma(dad[4], v, kbc[31]);
+          kbd[34] = fma(dac[1], v, kbd[34]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 11];
+          jab[i * 6 + 5] = fma(dcd[11], v, jab[i * 6 + 5]);
+          jcd[11] = fma(dab[5], v, jcd[11]);
+          kac[1] = fma(dbd[35], v, kac[1]);
+          kad[5] = fma(dbc[31], v, kad[5]);
+          kbc[31] = fma(dad[5], v, kbc[31]);
+          kbd[35] = fma(dac[1], v, kbd[35]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 12];
+          jab[i * 6 + 5] = fma(dcd[12], v, jab[i * 6 + 5]);
+          jcd[12] = fma(dab[5], v, jcd[12]);
+          kac[2] = fma(dbd[30], v, kac[2]);
+          kad[0] = fma(dbc[32], v, kad[0]);
+          kbc[32] = fma(dad[0], v, kbc[32]);
+          kbd[30] = fma(dac[2], v, kbd[30]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 13];
+          jab[i * 6 + 5] = fma(dcd[13], v, jab[i * 6 + 5]);
+          jcd[13] = fma(dab[5], v, jcd[13]);
+          kac[2] = fma(dbd[31], v, kac[2]);
+          kad[1] = fma(dbc[32], v, kad[1]);
+          kbc[32] = fma(dad[1], v, kbc[32]);
+          kbd[31] = fma(dac[2], v, kbd[31]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 14];
+          jab[i * 6 + 5] = fma(dcd[14], v, jab[i * 6 + 5]);
+          jcd[14] = fma(dab[5], v, jcd[14]);
+          kac[2] = fma(dbd[32], v, kac[2]);
+          kad[2] = fma(dbc[32], v, kad[2]);
+          kbc[32] = fma(dad[2], v, kbc[32]);
+          kbd[32] = fma(dac[2], v, kbd[32]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 15];
+          jab[i * 6 + 5] = fma(dcd[15], v, jab[i * 6 + 5]);
+          jcd[15] = fma(dab[5], v, jcd[15]);
+          kac[2] = fma(dbd[33], v, kac[2]);
+          kad[3] = fma(dbc[32], v, kad[3]);
+          kbc[32] = fma(dad[3], v, kbc[32]);
+          kbd[33] = fma(dac[2], v, kbd[33]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 16];
+          jab[i * 6 + 5] = fma(dcd[16], v, jab[i * 6 + 5]);
+          jcd[16] = fma(dab[5], v, jcd[16]);
+          kac[2] = fma(dbd[34], v, kac[2]);
+          kad[4] = fma(dbc[32], v, kad[4]);
+          kbc[32] = fma(dad[4], v, kbc[32]);
+          kbd[34] = fma(dac[2], v, kbd[34]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 17];
+          jab[i * 6 + 5] = fma(dcd[17], v, jab[i * 6 + 5]);
+          jcd[17] = fma(dab[5], v, jcd[17]);
+          kac[2] = fma(dbd[35], v, kac[2]);
+          kad[5] = fma(dbc[32], v, kad[5]);
+          kbc[32] = fma(dad[5], v, kbc[32]);
+          kbd[35] = fma(dac[2], v, kbd[35]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 18];
+          jab[i * 6 + 5] = fma(dcd[18], v, jab[i * 6 + 5]);
+          jcd[18] = fma(dab[5], v, jcd[18]);
+          kac[3] = fma(dbd[30], v, kac[3]);
+          kad[0] = fma(dbc[33], v, kad[0]);
+          kbc[33] = fma(dad[0], v, kbc[33]);
+          kbd[30] = fma(dac[3], v, kbd[30]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 19];
+          jab[i * 6 + 5] = fma(dcd[19], v, jab[i * 6 + 5]);
+          jcd[19] = fma(dab[5], v, jcd[19]);
+          kac[3] = fma(dbd[31], v, kac[3]);
+          kad[1] = fma(dbc[33], v, kad[1]);
+          kbc[33] = fma(dad[1], v, kbc[33]);
+          kbd[31] = fma(dac[3], v, kbd[31]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 20];
+          jab[i * 6 + 5] = fma(dcd[20], v, jab[i * 6 + 5]);
+          jcd[20] = fma(dab[5], v, jcd[20]);
+          kac[3] = fma(dbd[32], v, kac[3]);
+          kad[2] = fma(dbc[33], v, kad[2]);
+          kbc[33] = fma(dad[2], v, kbc[33]);
+          kbd[32] = fma(dac[3], v, kbd[32]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 21];
+          jab[i * 6 + 5] = fma(dcd[21], v, jab[i * 6 + 5]);
+          jcd[21] = fma(dab[5], v, jcd[21]);
+          kac[3] = fma(dbd[33], v, kac[3]);
+          kad[3] = fma(dbc[33], v, kad[3]);
+          kbc[33] = fma(dad[3], v, kbc[33]);
+          kbd[33] = fma(dac[3], v, kbd[33]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 22];
+          jab[i * 6 + 5] = fma(dcd[22], v, jab[i * 6 + 5]);
+          jcd[22] = fma(dab[5], v, jcd[22]);
+          kac[3] = fma(dbd[34], v, kac[3]);
+          kad[4] = fma(dbc[33], v, kad[4]);
+          kbc[33] = fma(dad[4], v, kbc[33]);
+          kbd[34] = fma(dac[3], v, kbd[34]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 23];
+          jab[i * 6 + 5] = fma(dcd[23], v, jab[i * 6 + 5]);
+          jcd[23] = fma(dab[5], v, jcd[23]);
+          kac[3] = fma(dbd[35], v, kac[3]);
+          kad[5] = fma(dbc[33], v, kad[5]);
+          kbc[33] = fma(dad[5], v, kbc[33]);
+          kbd[35] = fma(dac[3], v, kbd[35]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 24];
+          jab[i * 6 + 5] = fma(dcd[24], v, jab[i * 6 + 5]);
+          jcd[24] = fma(dab[5], v, jcd[24]);
+          kac[4] = fma(dbd[30], v, kac[4]);
+          kad[0] = fma(dbc[34], v, kad[0]);
+          kbc[34] = fma(dad[0], v, kbc[34]);
+          kbd[30] = fma(dac[4], v, kbd[30]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 25];
+          jab[i * 6 + 5] = fma(dcd[25], v, jab[i * 6 + 5]);
+          jcd[25] = fma(dab[5], v, jcd[25]);
+          kac[4] = fma(dbd[31], v, kac[4]);
+          kad[1] = fma(dbc[34], v, kad[1]);
+          kbc[34] = fma(dad[1], v, kbc[34]);
+          kbd[31] = fma(dac[4], v, kbd[31]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 26];
+          jab[i * 6 + 5] = fma(dcd[26], v, jab[i * 6 + 5]);
+          jcd[26] = fma(dab[5], v, jcd[26]);
+          kac[4] = fma(dbd[32], v, kac[4]);
+          kad[2] = fma(dbc[34], v, kad[2]);
+          kbc[34] = fma(dad[2], v, kbc[34]);
+          kbd[32] = fma(dac[4], v, kbd[32]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 27];
+          jab[i * 6 + 5] = fma(dcd[27], v, jab[i * 6 + 5]);
+          jcd[27] = fma(dab[5], v, jcd[27]);
+          kac[4] = fma(dbd[33], v, kac[4]);
+          kad[3] = fma(dbc[34], v, kad[3]);
+          kbc[34] = fma(dad[3], v, kbc[34]);
+          kbd[33] = fma(dac[4], v, kbd[33]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 28];
+          jab[i * 6 + 5] = fma(dcd[28], v, jab[i * 6 + 5]);
+          jcd[28] = fma(dab[5], v, jcd[28]);
+          kac[4] = fma(dbd[34], v, kac[4]);
+          kad[4] = fma(dbc[34], v, kad[4]);
+          kbc[34] = fma(dad[4], v, kbc[34]);
+          kbd[34] = fma(dac[4], v, kbd[34]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 29];
+          jab[i * 6 + 5] = fma(dcd[29], v, jab[i * 6 + 5]);
+          jcd[29] = fma(dab[5], v, jcd[29]);
+          kac[4] = fma(dbd[35], v, kac[4]);
+          kad[5] = fma(dbc[34], v, kad[5]);
+          kbc[34] = fma(dad[5], v, kbc[34]);
+          kbd[35] = fma(dac[4], v, kbd[35]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 30];
+          jab[i * 6 + 5] = fma(dcd[30], v, jab[i * 6 + 5]);
+          jcd[30] = fma(dab[5], v, jcd[30]);
+          kac[5] = fma(dbd[30], v, kac[5]);
+          kad[0] = fma(dbc[35], v, kad[0]);
+          kbc[35] = fma(dad[0], v, kbc[35]);
+          kbd[30] = fma(dac[5], v, kbd[30]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 31];
+          jab[i * 6 + 5] = fma(dcd[31], v, jab[i * 6 + 5]);
+          jcd[31] = fma(dab[5], v, jcd[31]);
+          kac[5] = fma(dbd[31], v, kac[5]);
+          kad[1] = fma(dbc[35], v, kad[1]);
+          kbc[35] = fma(dad[1], v, kbc[35]);
+          kbd[31] = fma(dac[5], v, kbd[31]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 32];
+          jab[i * 6 + 5] = fma(dcd[32], v, jab[i * 6 + 5]);
+          jcd[32] = fma(dab[5], v, jcd[32]);
+          kac[5] = fma(dbd[32], v, kac[5]);
+          kad[2] = fma(dbc[35], v, kad[2]);
+          kbc[35] = fma(dad[2], v, kbc[35]);
+          kbd[32] = fma(dac[5], v, kbd[32]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 33];
+          jab[i * 6 + 5] = fma(dcd[33], v, jab[i * 6 + 5]);
+          jcd[33] = fma(dab[5], v, jcd[33]);
+          kac[5] = fma(dbd[33], v, kac[5]);
+          kad[3] = fma(dbc[35], v, kad[3]);
+          kbc[35] = fma(dad[3], v, kbc[35]);
+          kbd[33] = fma(dac[5], v, kbd[33]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 34];
+          jab[i * 6 + 5] = fma(dcd[34], v, jab[i * 6 + 5]);
+          jcd[34] = fma(dab[5], v, jcd[34]);
+          kac[5] = fma(dbd[34], v, kac[5]);
+          kad[4] = fma(dbc[35], v, kad[4]);
+          kbc[35] = fma(dad[4], v, kbc[35]);
+          kbd[34] = fma(dac[5], v, kbd[34]); }
+        { const double v = f * res[(i * 6 + 5) * 36 + 35];
+          jab[i * 6 + 5] = fma(dcd[35], v, jab[i * 6 + 5]);
+          jcd[35] = fma(dab[5], v, jcd[35]);
+          kac[5] = fma(dbd[35], v, kac[5]);
+          kad[5] = fma(dbc[35], v, kad[5]);
+          kbc[35] = fma(dad[5], v, kbc[35]);
+          kbd[35] = fma(dac[5], v, kbd[35]); }
+#pragma unroll
+        for (int k = 0; k < 6; ++k) atomicAdd(&jk.K[(ib_.z + i) * n + ik_.z + k], kac[k]);
+#pragma unroll
+        for (int l = 0; l < 6; ++l) atomicAdd(&jk.K[(ib_.z + i) * n + ik_.w + l], kad[l]);
+    }
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) atomicAdd(&jk.K[(ib_.w + j) * n + ik_.z + k], kbc[j * 6 + k]);
+#pragma unroll
+        for (int l = 0; l < 6; ++l) atomicAdd(&jk.K[(ib_.w + j) * n + ik_.w + l], kbd[j * 6 + l]);
+    }
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+#pragma unroll
+        for (int l = 0; l < 6; ++l) atomicAdd(&jk.J[(ik_.z + k) * n + ik_.w + l], 2.0 * jcd[k * 6 + l]);
 }
 
 // Persistent work-queue kernel: each warp takes chunks (one bra pair, a run of consecutive
@@ -12657,6 +14212,11 @@ __global__ void __launch_bounds__(128) eri_queue_dddd(const EriQueue Q) {
         const int p = ch.x, cnt = ch.z & 0xffff, lg = (ch.z >> 16) & 7, lgj = (ch.z >> 20) & 7;
         const int W = 32 >> lg, kq = lane & (W - 1), s = lane >> (5 - lg);
         const int js = s & ((1 << lgj) - 1), is = s >> lgj;
+        double jab[JK ? 36 : 1];  // J/K digestion: the bra pair's J, over the chunk
+        if constexpr (JK) {
+#pragma unroll
+            for (int x = 0; x < 36; ++x) jab[x] = 0.0;
+        }
         for (int base = 0; base < cnt; base += W) {
         const int q = ch.y + base + kq;
         const bool live = base + kq < cnt;
@@ -12696,12 +14256,24 @@ __global__ void __launch_bounds__(128) eri_queue_dddd(const EriQueue Q) {
             double res[1296];
             hrr_dddd(Q.pairs, p, q, acc, res);
             if constexpr (JK) {
-                jk_dddd(Q.jk, __ldg(&Q.pairs.info[p]), __ldg(&Q.pairs.info[q]), p == q, res);
+                const int4 ib_ = __ldg(&Q.pairs.info[p]), ik_ = __ldg(&Q.pairs.info[q]);
+                jk_dddd(Q.jk, ib_, ik_, jk_weight(ib_.z == ib_.w, ik_.z == ik_.w, p == q), res, jab);
             } else {
                 store_dddd(Q.out + __ldg(&Q.mol_out[ch.w]), __ldg(&Q.pairs.info[p]), __ldg(&Q.pairs.info[q]),
                             p == q, res);
             }
         }
+        }
+        if constexpr (JK) {
+            // one addition per J_ab and chunk
+            const int4 ib_ = __ldg(&Q.pairs.info[p]);
+#pragma unroll
+            for (int x = 0; x < 36; ++x) {
+                double v = jab[x];
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+                if (lane == 0) atomicAdd(&Q.jk.J[(long long)(ib_.z + x / 6) * Q.jk.n + ib_.w + x % 6], 2.0 * v);
+            }
         }
     }
 }

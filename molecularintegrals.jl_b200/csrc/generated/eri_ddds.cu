@@ -1948,17 +1948,312 @@ __device__ __forceinline__ void store_ddds(double *__restrict__ out, const int4 
       if ((!dab || 5 >= 5) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[215]; }
 }
 
-// The quartet's unique integrals digested into J and K (molints_plan_jk) instead of stored.
-__device__ __noinline__ void jk_ddds(const JKOut &jk, const int4 ib_, const int4 ik_, bool same,
-                                      const double *__restrict__ res) {
-    const bool dab = ib_.z == ib_.w, dcd = ik_.z == ik_.w;
-    for (int x = 0; x < 216; ++x) {
-        const int ia = x / 36, ibb = (x / 6) % 6, ic = (x / 1) % 6, id = x % 1;
-        if ((dab && ia < ibb) || (dcd && ic < id)) continue;
-        const int i = ib_.z + ia, j = ib_.w + ibb, k = ik_.z + ic, l = ik_.w + id;
-        if (same && pair_index(i, j) < pair_index(k, l)) continue;
-        jk_add(jk, i, j, k, l, res[x]);
+// The quartet's share of J and K (molints_plan_jk, eri_common.cuh): every integral of the block,
+// times f, into one orientation of each target; J_ab stays in the lane (one bra pair per chunk).
+__device__ __forceinline__ void jk_ddds(const JKOut &jk, const int4 ib_, const int4 ik_, double f,
+                                         const double *__restrict__ res, double *__restrict__ jab) {
+    const long long n = jk.n;
+    const double *__restrict__ D = jk.D;
+    const double *__restrict__ Db = D + ib_.w * n, *__restrict__ Dc = D + ik_.z * n;
+    double dcd[6], dbc[36], dbd[6], jcd[6], kbc[36], kbd[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+#pragma unroll
+        for (int l = 0; l < 1; ++l) {
+            dcd[k * 1 + l] = __ldg(&Dc[k * n + ik_.w + l]);
+            jcd[k * 1 + l] = 0.0;
+        }
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            dbc[j * 6 + k] = __ldg(&Db[j * n + ik_.z + k]);
+            kbc[j * 6 + k] = 0.0;
+        }
+#pragma unroll
+        for (int l = 0; l < 1; ++l) {
+            dbd[j * 1 + l] = __ldg(&Db[j * n + ik_.w + l]);
+            kbd[j * 1 + l] = 0.0;
+        }
     }
+#pragma unroll 1
+    for (int i = 0; i < 6; ++i) {
+        const double *__restrict__ Da = D + (ib_.z + i) * n;
+        double dab[6], dac[6], dad[1], kac[6], kad[1];
+#pragma unroll
+        for (int j = 0; j < 6; ++j) dab[j] = __ldg(&Da[ib_.w + j]);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) { dac[k] = __ldg(&Da[ik_.z + k]); kac[k] = 0.0; }
+#pragma unroll
+        for (int l = 0; l < 1; ++l) { dad[l] = __ldg(&Da[ik_.w + l]); kad[l] = 0.0; }
+        { const double v = f * res[(i * 6 + 0) * 6 + 0];
+          jab[i * 6 + 0] = fma(dcd[0], v, jab[i * 6 + 0]);
+          jcd[0] = fma(dab[0], v, jcd[0]);
+          kac[0] = fma(dbd[0], v, kac[0]);
+          kad[0] = fma(dbc[0], v, kad[0]);
+          kbc[0] = fma(dad[0], v, kbc[0]);
+          kbd[0] = fma(dac[0], v, kbd[0]); }
+        { const double v = f * res[(i * 6 + 0) * 6 + 1];
+          jab[i * 6 + 0] = fma(dcd[1], v, jab[i * 6 + 0]);
+          jcd[1] = fma(dab[0], v, jcd[1]);
+          kac[1] = fma(dbd[0], v, kac[1]);
+          kad[0] = fma(dbc[1], v, kad[0]);
+          kbc[1] = fma(dad[0], v, kbc[1]);
+          kbd[0] = fma(dac[1], v, kbd[0]); }
+        { const double v = f * res[(i * 6 + 0) * 6 + 2];
+          jab[i * 6 + 0] = fma(dcd[2], v, jab[i * 6 + 0]);
+          jcd[2] = fma(dab[0], v, jcd[2]);
+          kac[2] = fma(dbd[0], v, kac[2]);
+          kad[0] = fma(dbc[2], v, kad[0]);
+          kbc[2] = fma(dad[0], v, kbc[2]);
+          kbd[0] = fma(dac[2], v, kbd[0]); }
+        { const double v = f * res[(i * 6 + 0) * 6 + 3];
+          jab[i * 6 + 0] = fma(dcd[3], v, jab[i * 6 + 0]);
+          jcd[3] = fma(dab[0], v, jcd[3]);
+          kac[3] = fma(dbd[0], v, kac[3]);
+          kad[0] = fma(dbc[3], v, kad[0]);
+          kbc[3] = fma(dad[0], v, kbc[3]);
+          kbd[0] = fma(dac[3], v, kbd[0]); }
+        { const double v = f * res[(i * 6 + 0) * 6 + 4];
+          jab[i * 6 + 0] = fma(dcd[4], v, jab[i * 6 + 0]);
+          jcd[4] = fma(dab[0], v, jcd[4]);
+          kac[4] = fma(dbd[0], v, kac[4]);
+          kad[0] = fma(dbc[4], v, kad[0]);
+          kbc[4] = fma(dad[0], v, kbc[4]);
+          kbd[0] = fma(dac[4], v, kbd[0]); }
+        { const double v = f * res[(i * 6 + 0) * 6 + 5];
+          jab[i * 6 + 0] = fma(dcd[5], v, jab[i * 6 + 0]);
+          jcd[5] = fma(dab[0], v, jcd[5]);
+          kac[5] = fma(dbd[0], v, kac[5]);
+          kad[0] = fma(dbc[5], v, kad[0]);
+          kbc[5] = fma(dad[0], v, kbc[5]);
+          kbd[0] = fma(dac[5], v, kbd[0]); }
+        { const double v = f * res[(i * 6 + 1) * 6 + 0];
+          jab[i * 6 + 1] = fma(dcd[0], v, jab[i * 6 + 1]);
+          jcd[0] = fma(dab[1], v, jcd[0]);
+          kac[0] = fma(dbd[1], v, kac[0]);
+          kad[0] = fma(dbc[6], v, kad[0]);
+          kbc[6] = fma(dad[0], v, kbc[6]);
+          kbd[1] = fma(dac[0], v, kbd[1]); }
+        { const double v = f * res[(i * 6 + 1) * 6 + 1];
+          jab[i * 6 + 1] = fma(dcd[1], v, jab[i * 6 + 1]);
+          jcd[1] = fma(dab[1], v, jcd[1]);
+          kac[1] = fma(dbd[1], v, kac[1]);
+          kad[0] = fma(dbc[7], v, kad[0]);
+          kbc[7] = fma(dad[0], v, kbc[7]);
+          kbd[1] = fma(dac[1], v, kbd[1]); }
+        { const double v = f * res[(i * 6 + 1) * 6 + 2];
+          jab[i * 6 + 1] = fma(dcd[2], v, jab[i * 6 + 1]);
+          jcd[2] = fma(dab[1], v, jcd[2]);
+          kac[2] = fma(dbd[1], v, kac[2]);
+          kad[0] = fma(dbc[8], v, kad[0]);
+          kbc[8] = fma(dad[0], v, kbc[8]);
+          kbd[1] = fma(dac[2], v, kbd[1]); }
+        { const double v = f * res[(i * 6 + 1) * 6 + 3];
+          jab[i * 6 + 1] = fma(dcd[3], v, jab[i * 6 + 1]);
+          jcd[3] = fma(dab[1], v, jcd[3]);
+          kac[3] = fma(dbd[1], v, kac[3]);
+          kad[0] = fma(dbc[9], v, kad[0]);
+          kbc[9] = fma(dad[0], v, kbc[9]);
+          kbd[1] = fma(dac[3], v, kbd[1]); }
+        { const double v = f * res[(i * 6 + 1) * 6 + 4];
+          jab[i * 6 + 1] = fma(dcd[4], v, jab[i * 6 + 1]);
+          jcd[4] = fma(dab[1], v, jcd[4]);
+          kac[4] = fma(dbd[1], v, kac[4]);
+          kad[0] = fma(dbc[10], v, kad[0]);
+          kbc[10] = fma(dad[0], v, kbc[10]);
+          kbd[1] = fma(dac[4], v, kbd[1]); }
+        { const double v = f * res[(i * 6 + 1) * 6 + 5];
+          jab[i * 6 + 1] = fma(dcd[5], v, jab[i * 6 + 1]);
+          jcd[5] = fma(dab[1], v, jcd[5]);
+          kac[5] = fma(dbd[1], v, kac[5]);
+          kad[0] = fma(dbc[11], v, kad[0]);
+          kbc[11] = fma(dad[0], v, kbc[11]);
+          kbd[1] = fma(dac[5], v, kbd[1]); }
+        { const double v = f * res[(i * 6 + 2) * 6 + 0];
+          jab[i * 6 + 2] = fma(dcd[0], v, jab[i * 6 + 2]);
+          jcd[0] = fma(dab[2], v, jcd[0]);
+          kac[0] = fma(dbd[2], v, kac[0]);
+          kad[0] = fma(dbc[12], v, kad[0]);
+          kbc[12] = fma(dad[0], v, kbc[12]);
+          kbd[2] = fma(dac[0], v, kbd[2]); }
+        { const double v = f * res[(i * 6 + 2) * 6 + 1];
+          jab[i * 6 + 2] = fma(dcd[1], v, jab[i * 6 + 2]);
+          jcd[1] = fma(dab[2], v, jcd[1]);
+          kac[1] = fma(dbd[2], v, kac[1]);
+          kad[0] = fma(dbc[13], v, kad[0]);
+          kbc[13] = fma(dad[0], v, kbc[13]);
+          kbd[2] = fma(dac[1], v, kbd[2]); }
+        { const double v = f * res[(i * 6 + 2) * 6 + 2];
+          jab[i * 6 + 2] = fma(dcd[2], v, jab[i * 6 + 2]);
+          jcd[2] = fma(dab[2], v, jcd[2]);
+          kac[2] = fma(dbd[2], v, kac[2]);
+          kad[0] = fma(dbc[14], v, kad[0]);
+          kbc[14] = fma(dad[0], v, kbc[14]);
+          kbd[2] = fma(dac[2], v, kbd[2]); }
+        { const double v = f * res[(i * 6 + 2) * 6 + 3];
+          jab[i * 6 + 2] = fma(dcd[3], v, jab[i * 6 + 2]);
+          jcd[3] = fma(dab[2], v, jcd[3]);
+          kac[3] = fma(dbd[2], v, kac[3]);
+          kad[0] = fma(dbc[15], v, kad[0]);
+          kbc[15] = fma(dad[0], v, kbc[15]);
+          kbd[2] = fma(dac[3], v, kbd[2]); }
+        { const double v = f * res[(i * 6 + 2) * 6 + 4];
+          jab[i * 6 + 2] = fma(dcd[4], v, jab[i * 6 + 2]);
+          jcd[4] = fma(dab[2], v, jcd[4]);
+          kac[4] = fma(dbd[2], v, kac[4]);
+          kad[0] = fma(dbc[16], v, kad[0]);
+          kbc[16] = fma(dad[0], v, kbc[16]);
+          kbd[2] = fma(dac[4], v, kbd[2]); }
+        { const double v = f * res[(i * 6 + 2) * 6 + 5];
+          jab[i * 6 + 2] = fma(dcd[5], v, jab[i * 6 + 2]);
+          jcd[5] = fma(dab[2], v, jcd[5]);
+          kac[5] = fma(dbd[2], v, kac[5]);
+          kad[0] = fma(dbc[17], v, kad[0]);
+          kbc[17] = fma(dad[0], v, kbc[17]);
+          kbd[2] = fma(dac[5], v, kbd[2]); }
+        { const double v = f * res[(i * 6 + 3) * 6 + 0];
+          jab[i * 6 + 3] = fma(dcd[0], v, jab[i * 6 + 3]);
+          jcd[0] = fma(dab[3], v, jcd[0]);
+          kac[0] = fma(dbd[3], v, kac[0]);
+          kad[0] = fma(dbc[18], v, kad[0]);
+          kbc[18] = fma(dad[0], v, kbc[18]);
+          kbd[3] = fma(dac[0], v, kbd[3]); }
+        { const double v = f * res[(i * 6 + 3) * 6 + 1];
+          jab[i * 6 + 3] = fma(dcd[1], v, jab[i * 6 + 3]);
+          jcd[1] = fma(dab[3], v, jcd[1]);
+          kac[1] = fma(dbd[3], v, kac[1]);
+          kad[0] = fma(dbc[19], v, kad[0]);
+          kbc[19] = fma(dad[0], v, kbc[19]);
+          kbd[3] = fma(dac[1], v, kbd[3]); }
+        { const double v = f * res[(i * 6 + 3) * 6 + 2];
+          jab[i * 6 + 3] = fma(dcd[2], v, jab[i * 6 + 3]);
+          jcd[2] = fma(dab[3], v, jcd[2]);
+          kac[2] = fma(dbd[3], v, kac[2]);
+          kad[0] = fma(dbc[20], v, kad[0]);
+          kbc[20] = fma(dad[0], v, kbc[20]);
+          kbd[3] = fma(dac[2], v, kbd[3]); }
+        { const double v = f * res[(i * 6 + 3) * 6 + 3];
+          jab[i * 6 + 3] = fma(dcd[3], v, jab[i * 6 + 3]);
+          jcd[3] = fma(dab[3], v, jcd[3]);
+          kac[3] = fma(dbd[3], v, kac[3]);
+          kad[0] = fma(dbc[21], v, kad[0]);
+          kbc[21] = fma(dad[0], v, kbc[21]);
+          kbd[3] = fma(dac[3], v, kbd[3]); }
+        { const double v = f * res[(i * 6 + 3) * 6 + 4];
+          jab[i * 6 + 3] = fma(dcd[4], v, jab[i * 6 + 3]);
+          jcd[4] = fma(dab[3], v, jcd[4]);
+          kac[4] = fma(dbd[3], v, kac[4]);
+          kad[0] = fma(dbc[22], v, kad[0]);
+          kbc[22] = fma(dad[0], v, kbc[22]);
+          kbd[3] = fma(dac[4], v, kbd[3]); }
+        { const double v = f * res[(i * 6 + 3) * 6 + 5];
+          jab[i * 6 + 3] = fma(dcd[5], v, jab[i * 6 + 3]);
+          jcd[5] = fma(dab[3], v, jcd[5]);
+          kac[5] = fma(dbd[3], v, kac[5]);
+          kad[0] = fma(dbc[23], v, kad[0]);
+          kbc[23] = fma(dad[0], v, kbc[23]);
+          kbd[3] = fma(dac[5], v, kbd[3]); }
+        { const double v = f * res[(i * 6 + 4) * 6 + 0];
+          jab[i * 6 + 4] = fma(dcd[0], v, jab[i * 6 + 4]);
+          jcd[0] = fma(dab[4], v, jcd[0]);
+          kac[0] = fma(dbd[4], v, kac[0]);
+          kad[0] = fma(dbc[24], v, kad[0]);
+          kbc[24] = fma(dad[0], v, kbc[24]);
+          kbd[4] = fma(dac[0], v, kbd[4]); }
+        { const double v = f * res[(i * 6 + 4) * 6 + 1];
+          jab[i * 6 + 4] = fma(dcd[1], v, jab[i * 6 + 4]);
+          jcd[1] = fma(dab[4], v, jcd[1]);
+          kac[1] = fma(dbd[4], v, kac[1]);
+          kad[0] = fma(dbc[25], v, kad[0]);
+          kbc[25] = fma(dad[0], v, kbc[25]);
+          kbd[4] = fma(dac[1], v, kbd[4]); }
+        { const double v = f * res[(i * 6 + 4) * 6 + 2];
+          jab[i * 6 + 4] = fma(dcd[2], v, jab[i * 6 + 4]);
+          jcd[2] = fma(dab[4], v, jcd[2]);
+          kac[2] = fma(dbd[4], v, kac[2]);
+          kad[0] = fma(dbc[26], v, kad[0]);
+          kbc[26] = fma(dad[0], v, kbc[26]);
+          kbd[4] = fma(dac[2], v, kbd[4]); }
+        { const double v = f * res[(i * 6 + 4) * 6 + 3];
+          jab[i * 6 + 4] = fma(dcd[3], v, jab[i * 6 + 4]);
+          jcd[3] = fma(dab[4], v, jcd[3]);
+          kac[3] = fma(dbd[4], v, kac[3]);
+          kad[0] = fma(dbc[27], v, kad[0]);
+          kbc[27] = fma(dad[0], v, kbc[27]);
+          kbd[4] = fma(dac[3], v, kbd[4]); }
+        { const double v = f * res[(i * 6 + 4) * 6 + 4];
+          jab[i * 6 + 4] = fma(dcd[4], v, jab[i * 6 + 4]);
+          jcd[4] = fma(dab[4], v, jcd[4]);
+          kac[4] = fma(dbd[4], v, kac[4]);
+          kad[0] = fma(dbc[28], v, kad[0]);
+          kbc[28] = fma(dad[0], v, kbc[28]);
+          kbd[4] = fma(dac[4], v, kbd[4]); }
+        { const double v = f * res[(i * 6 + 4) * 6 + 5];
+          jab[i * 6 + 4] = fma(dcd[5], v, jab[i * 6 + 4]);
+          jcd[5] = fma(dab[4], v, jcd[5]);
+          kac[5] = fma(dbd[4], v, kac[5]);
+          kad[0] = fma(dbc[29], v, kad[0]);
+          kbc[29] = fma(dad[0], v, kbc[29]);
+          kbd[4] = fma(dac[5], v, kbd[4]); }
+        { const double v = f * res[(i * 6 + 5) * 6 + 0];
+          jab[i * 6 + 5] = fma(dcd[0], v, jab[i * 6 + 5]);
+          jcd[0] = fma(dab[5], v, jcd[0]);
+          kac[0] = fma(dbd[5], v, kac[0]);
+          kad[0] = fma(dbc[30], v, kad[0]);
+          kbc[30] = fma(dad[0], v, kbc[30]);
+          kbd[5] = fma(dac[0], v, kbd[5]); }
+        { const double v = f * res[(i * 6 + 5) * 6 + 1];
+          jab[i * 6 + 5] = fma(dcd[1], v, jab[i * 6 + 5]);
+          jcd[1] = fma(dab[5], v, jcd[1]);
+          kac[1] = fma(dbd[5], v, kac[1]);
+          kad[0] = fma(dbc[31], v, kad[0]);
+          kbc[31] = fma(dad[0], v, kbc[31]);
+          kbd[5] = fma(dac[1], v, kbd[5]); }
+        { const double v = f * res[(i * 6 + 5) * 6 + 2];
+          jab[i * 6 + 5] = fma(dcd[2], v, jab[i * 6 + 5]);
+          jcd[2] = fma(dab[5], v, jcd[2]);
+          kac[2] = fma(dbd[5], v, kac[2]);
+          kad[0] = fma(dbc[32], v, kad[0]);
+          kbc[32] = fma(dad[0], v, kbc[32]);
+          kbd[5] = fma(dac[2], v, kbd[5]); }
+        { const double v = f * res[(i * 6 + 5) * 6 + 3];
+          jab[i * 6 + 5] = fma(dcd[3], v, jab[i * 6 + 5]);
+          jcd[3] = fma(dab[5], v, jcd[3]);
+          kac[3] = fma(dbd[5], v, kac[3]);
+          kad[0] = fma(dbc[33], v, kad[0]);
+          kbc[33] = fma(dad[0], v, kbc[33]);
+          kbd[5] = fma(dac[3], v, kbd[5]); }
+        { const double v = f * res[(i * 6 + 5) * 6 + 4];
+          jab[i * 6 + 5] = fma(dcd[4], v, jab[i * 6 + 5]);
+          jcd[4] = fma(dab[5], v, jcd[4]);
+          kac[4] = fma(dbd[5], v, kac[4]);
+          kad[0] = fma(dbc[34], v, kad[0]);
+          kbc[34] = fma(dad[0], v, kbc[34]);
+          kbd[5] = fma(dac[4], v, kbd[5]); }
+        { const double v = f * res[(i * 6 + 5) * 6 + 5];
+          jab[i * 6 + 5] = fma(dcd[5], v, jab[i * 6 + 5]);
+          jcd[5] = fma(dab[5], v, jcd[5]);
+          kac[5] = fma(dbd[5], v, kac[5]);
+          kad[0] = fma(dbc[35], v, kad[0]);
+          kbc[35] = fma(dad[0], v, kbc[35]);
+          kbd[5] = fma(dac[5], v, kbd[5]); }
+#pragma unroll
+        for (int k = 0; k < 6; ++k) atomicAdd(&jk.K[(ib_.z + i) * n + ik_.z + k], kac[k]);
+#pragma unroll
+        for (int l = 0; l < 1; ++l) atomicAdd(&jk.K[(ib_.z + i) * n + ik_.w + l], kad[l]);
+    }
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) atomicAdd(&jk.K[(ib_.w + j) * n + ik_.z + k], kbc[j * 6 + k]);
+#pragma unroll
+        for (int l = 0; l < 1; ++l) atomicAdd(&jk.K[(ib_.w + j) * n + ik_.w + l], kbd[j * 1 + l]);
+    }
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+#pragma unroll
+        for (int l = 0; l < 1; ++l) atomicAdd(&jk.J[(ik_.z + k) * n + ik_.w + l], 2.0 * jcd[k * 1 + l]);
 }
 
 // Persistent work-queue kernel: each warp takes chunks (one bra pair, a run of consecutive
@@ -1984,6 +2279,11 @@ __global__ void __launch_bounds__(128) eri_queue_ddds(const EriQueue Q) {
         const int p = ch.x, cnt = ch.z & 0xffff, lg = (ch.z >> 16) & 7, lgj = (ch.z >> 20) & 7;
         const int W = 32 >> lg, kq = lane & (W - 1), s = lane >> (5 - lg);
         const int js = s & ((1 << lgj) - 1), is = s >> lgj;
+        double jab[JK ? 36 : 1];  // J/K digestion: the bra pair's J, over the chunk
+        if constexpr (JK) {
+#pragma unroll
+            for (int x = 0; x < 36; ++x) jab[x] = 0.0;
+        }
         for (int base = 0; base < cnt; base += W) {
         const int q = ch.y + base + kq;
         const bool live = base + kq < cnt;
@@ -2023,12 +2323,24 @@ __global__ void __launch_bounds__(128) eri_queue_ddds(const EriQueue Q) {
             double res[216];
             hrr_ddds(Q.pairs, p, q, acc, res);
             if constexpr (JK) {
-                jk_ddds(Q.jk, __ldg(&Q.pairs.info[p]), __ldg(&Q.pairs.info[q]), p == q, res);
+                const int4 ib_ = __ldg(&Q.pairs.info[p]), ik_ = __ldg(&Q.pairs.info[q]);
+                jk_ddds(Q.jk, ib_, ik_, jk_weight(ib_.z == ib_.w, ik_.z == ik_.w, p == q), res, jab);
             } else {
                 store_ddds(Q.out + __ldg(&Q.mol_out[ch.w]), __ldg(&Q.pairs.info[p]), __ldg(&Q.pairs.info[q]),
                             p == q, res);
             }
         }
+        }
+        if constexpr (JK) {
+            // one addition per J_ab and chunk
+            const int4 ib_ = __ldg(&Q.pairs.info[p]);
+#pragma unroll
+            for (int x = 0; x < 36; ++x) {
+                double v = jab[x];
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+                if (lane == 0) atomicAdd(&Q.jk.J[(long long)(ib_.z + x / 6) * Q.jk.n + ib_.w + x % 6], 2.0 * v);
+            }
         }
     }
 }

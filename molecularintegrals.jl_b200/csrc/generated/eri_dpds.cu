@@ -905,17 +905,186 @@ __device__ __forceinline__ void store_dpds(double *__restrict__ out, const int4 
       if (true && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[107]; }
 }
 
-// The quartet's unique integrals digested into J and K (molints_plan_jk) instead of stored.
-__device__ __noinline__ void jk_dpds(const JKOut &jk, const int4 ib_, const int4 ik_, bool same,
-                                      const double *__restrict__ res) {
-    const bool dab = ib_.z == ib_.w, dcd = ik_.z == ik_.w;
-    for (int x = 0; x < 108; ++x) {
-        const int ia = x / 18, ibb = (x / 6) % 3, ic = (x / 1) % 6, id = x % 1;
-        if ((dab && ia < ibb) || (dcd && ic < id)) continue;
-        const int i = ib_.z + ia, j = ib_.w + ibb, k = ik_.z + ic, l = ik_.w + id;
-        if (same && pair_index(i, j) < pair_index(k, l)) continue;
-        jk_add(jk, i, j, k, l, res[x]);
+// The quartet's share of J and K (molints_plan_jk, eri_common.cuh): every integral of the block,
+// times f, into one orientation of each target; J_ab stays in the lane (one bra pair per chunk).
+__device__ __forceinline__ void jk_dpds(const JKOut &jk, const int4 ib_, const int4 ik_, double f,
+                                         const double *__restrict__ res, double *__restrict__ jab) {
+    const long long n = jk.n;
+    const double *__restrict__ D = jk.D;
+    const double *__restrict__ Db = D + ib_.w * n, *__restrict__ Dc = D + ik_.z * n;
+    double dcd[6], dbc[18], dbd[3], jcd[6], kbc[18], kbd[3];
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+#pragma unroll
+        for (int l = 0; l < 1; ++l) {
+            dcd[k * 1 + l] = __ldg(&Dc[k * n + ik_.w + l]);
+            jcd[k * 1 + l] = 0.0;
+        }
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            dbc[j * 6 + k] = __ldg(&Db[j * n + ik_.z + k]);
+            kbc[j * 6 + k] = 0.0;
+        }
+#pragma unroll
+        for (int l = 0; l < 1; ++l) {
+            dbd[j * 1 + l] = __ldg(&Db[j * n + ik_.w + l]);
+            kbd[j * 1 + l] = 0.0;
+        }
     }
+#pragma unroll 1
+    for (int i = 0; i < 6; ++i) {
+        const double *__restrict__ Da = D + (ib_.z + i) * n;
+        double dab[3], dac[6], dad[1], kac[6], kad[1];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) dab[j] = __ldg(&Da[ib_.w + j]);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) { dac[k] = __ldg(&Da[ik_.z + k]); kac[k] = 0.0; }
+#pragma unroll
+        for (int l = 0; l < 1; ++l) { dad[l] = __ldg(&Da[ik_.w + l]); kad[l] = 0.0; }
+        { const double v = f * res[(i * 3 + 0) * 6 + 0];
+          jab[i * 3 + 0] = fma(dcd[0], v, jab[i * 3 + 0]);
+          jcd[0] = fma(dab[0], v, jcd[0]);
+          kac[0] = fma(dbd[0], v, kac[0]);
+          kad[0] = fma(dbc[0], v, kad[0]);
+          kbc[0] = fma(dad[0], v, kbc[0]);
+          kbd[0] = fma(dac[0], v, kbd[0]); }
+        { const double v = f * res[(i * 3 + 0) * 6 + 1];
+          jab[i * 3 + 0] = fma(dcd[1], v, jab[i * 3 + 0]);
+          jcd[1] = fma(dab[0], v, jcd[1]);
+          kac[1] = fma(dbd[0], v, kac[1]);
+          kad[0] = fma(dbc[1], v, kad[0]);
+          kbc[1] = fma(dad[0], v, kbc[1]);
+          kbd[0] = fma(dac[1], v, kbd[0]); }
+        { const double v = f * res[(i * 3 + 0) * 6 + 2];
+          jab[i * 3 + 0] = fma(dcd[2], v, jab[i * 3 + 0]);
+          jcd[2] = fma(dab[0], v, jcd[2]);
+          kac[2] = fma(dbd[0], v, kac[2]);
+          kad[0] = fma(dbc[2], v, kad[0]);
+          kbc[2] = fma(dad[0], v, kbc[2]);
+          kbd[0] = fma(dac[2], v, kbd[0]); }
+        { const double v = f * res[(i * 3 + 0) * 6 + 3];
+          jab[i * 3 + 0] = fma(dcd[3], v, jab[i * 3 + 0]);
+          jcd[3] = fma(dab[0], v, jcd[3]);
+          kac[3] = fma(dbd[0], v, kac[3]);
+          kad[0] = fma(dbc[3], v, kad[0]);
+          kbc[3] = fma(dad[0], v, kbc[3]);
+          kbd[0] = fma(dac[3], v, kbd[0]); }
+        { const double v = f * res[(i * 3 + 0) * 6 + 4];
+          jab[i * 3 + 0] = fma(dcd[4], v, jab[i * 3 + 0]);
+          jcd[4] = fma(dab[0], v, jcd[4]);
+          kac[4] = fma(dbd[0], v, kac[4]);
+          kad[0] = fma(dbc[4], v, kad[0]);
+          kbc[4] = fma(dad[0], v, kbc[4]);
+          kbd[0] = fma(dac[4], v, kbd[0]); }
+        { const double v = f * res[(i * 3 + 0) * 6 + 5];
+          jab[i * 3 + 0] = fma(dcd[5], v, jab[i * 3 + 0]);
+          jcd[5] = fma(dab[0], v, jcd[5]);
+          kac[5] = fma(dbd[0], v, kac[5]);
+          kad[0] = fma(dbc[5], v, kad[0]);
+          kbc[5] = fma(dad[0], v, kbc[5]);
+          kbd[0] = fma(dac[5], v, kbd[0]); }
+        { const double v = f * res[(i * 3 + 1) * 6 + 0];
+          jab[i * 3 + 1] = fma(dcd[0], v, jab[i * 3 + 1]);
+          jcd[0] = fma(dab[1], v, jcd[0]);
+          kac[0] = fma(dbd[1], v, kac[0]);
+          kad[0] = fma(dbc[6], v, kad[0]);
+          kbc[6] = fma(dad[0], v, kbc[6]);
+          kbd[1] = fma(dac[0], v, kbd[1]); }
+        { const double v = f * res[(i * 3 + 1) * 6 + 1];
+          jab[i * 3 + 1] = fma(dcd[1], v, jab[i * 3 + 1]);
+          jcd[1] = fma(dab[1], v, jcd[1]);
+          kac[1] = fma(dbd[1], v, kac[1]);
+          kad[0] = fma(dbc[7], v, kad[0]);
+          kbc[7] = fma(dad[0], v, kbc[7]);
+          kbd[1] = fma(dac[1], v, kbd[1]); }
+        { const double v = f * res[(i * 3 + 1) * 6 + 2];
+          jab[i * 3 + 1] = fma(dcd[2], v, jab[i * 3 + 1]);
+          jcd[2] = fma(dab[1], v, jcd[2]);
+          kac[2] = fma(dbd[1], v, kac[2]);
+          kad[0] = fma(dbc[8], v, kad[0]);
+          kbc[8] = fma(dad[0], v, kbc[8]);
+          kbd[1] = fma(dac[2], v, kbd[1]); }
+        { const double v = f * res[(i * 3 + 1) * 6 + 3];
+          jab[i * 3 + 1] = fma(dcd[3], v, jab[i * 3 + 1]);
+          jcd[3] = fma(dab[1], v, jcd[3]);
+          kac[3] = fma(dbd[1], v, kac[3]);
+          kad[0] = fma(dbc[9], v, kad[0]);
+          kbc[9] = fma(dad[0], v, kbc[9]);
+          kbd[1] = fma(dac[3], v, kbd[1]); }
+        { const double v = f * res[(i * 3 + 1) * 6 + 4];
+          jab[i * 3 + 1] = fma(dcd[4], v, jab[i * 3 + 1]);
+          jcd[4] = fma(dab[1], v, jcd[4]);
+          kac[4] = fma(dbd[1], v, kac[4]);
+          kad[0] = fma(dbc[10], v, kad[0]);
+          kbc[10] = fma(dad[0], v, kbc[10]);
+          kbd[1] = fma(dac[4], v, kbd[1]); }
+        { const double v = f * res[(i * 3 + 1) * 6 + 5];
+          jab[i * 3 + 1] = fma(dcd[5], v, jab[i * 3 + 1]);
+          jcd[5] = fma(dab[1], v, jcd[5]);
+          kac[5] = fma(dbd[1], v, kac[5]);
+          kad[0] = fma(dbc[11], v, kad[0]);
+          kbc[11] = fma(dad[0], v, kbc[11]);
+          kbd[1] = fma(dac[5], v, kbd[1]); }
+        { const double v = f * res[(i * 3 + 2) * 6 + 0];
+          jab[i * 3 + 2] = fma(dcd[0], v, jab[i * 3 + 2]);
+          jcd[0] = fma(dab[2], v, jcd[0]);
+          kac[0] = fma(dbd[2], v, kac[0]);
+          kad[0] = fma(dbc[12], v, kad[0]);
+          kbc[12] = fma(dad[0], v, kbc[12]);
+          kbd[2] = fma(dac[0], v, kbd[2]); }
+        { const double v = f * res[(i * 3 + 2) * 6 + 1];
+          jab[i * 3 + 2] = fma(dcd[1], v, jab[i * 3 + 2]);
+          jcd[1] = fma(dab[2], v, jcd[1]);
+          kac[1] = fma(dbd[2], v, kac[1]);
+          kad[0] = fma(dbc[13], v, kad[0]);
+          kbc[13] = fma(dad[0], v, kbc[13]);
+          kbd[2] = fma(dac[1], v, kbd[2]); }
+        { const double v = f * res[(i * 3 + 2) * 6 + 2];
+          jab[i * 3 + 2] = fma(dcd[2], v, jab[i * 3 + 2]);
+          jcd[2] = fma(dab[2], v, jcd[2]);
+          kac[2] = fma(dbd[2], v, kac[2]);
+          kad[0] = fma(dbc[14], v, kad[0]);
+          kbc[14] = fma(dad[0], v, kbc[14]);
+          kbd[2] = fma(dac[2], v, kbd[2]); }
+        { const double v = f * res[(i * 3 + 2) * 6 + 3];
+          jab[i * 3 + 2] = fma(dcd[3], v, jab[i * 3 + 2]);
+          jcd[3] = fma(dab[2], v, jcd[3]);
+          kac[3] = fma(dbd[2], v, kac[3]);
+          kad[0] = fma(dbc[15], v, kad[0]);
+          kbc[15] = fma(dad[0], v, kbc[15]);
+          kbd[2] = fma(dac[3], v, kbd[2]); }
+        { const double v = f * res[(i * 3 + 2) * 6 + 4];
+          jab[i * 3 + 2] = fma(dcd[4], v, jab[i * 3 + 2]);
+          jcd[4] = fma(dab[2], v, jcd[4]);
+          kac[4] = fma(dbd[2], v, kac[4]);
+          kad[0] = fma(dbc[16], v, kad[0]);
+          kbc[16] = fma(dad[0], v, kbc[16]);
+          kbd[2] = fma(dac[4], v, kbd[2]); }
+        { const double v = f * res[(i * 3 + 2) * 6 + 5];
+          jab[i * 3 + 2] = fma(dcd[5], v, jab[i * 3 + 2]);
+          jcd[5] = fma(dab[2], v, jcd[5]);
+          kac[5] = fma(dbd[2], v, kac[5]);
+          kad[0] = fma(dbc[17], v, kad[0]);
+          kbc[17] = fma(dad[0], v, kbc[17]);
+          kbd[2] = fma(dac[5], v, kbd[2]); }
+#pragma unroll
+        for (int k = 0; k < 6; ++k) atomicAdd(&jk.K[(ib_.z + i) * n + ik_.z + k], kac[k]);
+#pragma unroll
+        for (int l = 0; l < 1; ++l) atomicAdd(&jk.K[(ib_.z + i) * n + ik_.w + l], kad[l]);
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) atomicAdd(&jk.K[(ib_.w + j) * n + ik_.z + k], kbc[j * 6 + k]);
+#pragma unroll
+        for (int l = 0; l < 1; ++l) atomicAdd(&jk.K[(ib_.w + j) * n + ik_.w + l], kbd[j * 1 + l]);
+    }
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+#pragma unroll
+        for (int l = 0; l < 1; ++l) atomicAdd(&jk.J[(ik_.z + k) * n + ik_.w + l], 2.0 * jcd[k * 1 + l]);
 }
 
 // Persistent work-queue kernel: each warp takes chunks (one bra pair, a run of consecutive
@@ -941,6 +1110,11 @@ __global__ void __launch_bounds__(128) eri_queue_dpds(const EriQueue Q) {
         const int p = ch.x, cnt = ch.z & 0xffff, lg = (ch.z >> 16) & 7, lgj = (ch.z >> 20) & 7;
         const int W = 32 >> lg, kq = lane & (W - 1), s = lane >> (5 - lg);
         const int js = s & ((1 << lgj) - 1), is = s >> lgj;
+        double jab[JK ? 18 : 1];  // J/K digestion: the bra pair's J, over the chunk
+        if constexpr (JK) {
+#pragma unroll
+            for (int x = 0; x < 18; ++x) jab[x] = 0.0;
+        }
         for (int base = 0; base < cnt; base += W) {
         const int q = ch.y + base + kq;
         const bool live = base + kq < cnt;
@@ -983,12 +1157,24 @@ __global__ void __launch_bounds__(128) eri_queue_dpds(const EriQueue Q) {
             double res[108];
             hrr_dpds(Q.pairs, p, q, acc, res);
             if constexpr (JK) {
-                jk_dpds(Q.jk, __ldg(&Q.pairs.info[p]), __ldg(&Q.pairs.info[q]), p == q, res);
+                const int4 ib_ = __ldg(&Q.pairs.info[p]), ik_ = __ldg(&Q.pairs.info[q]);
+                jk_dpds(Q.jk, ib_, ik_, jk_weight(ib_.z == ib_.w, ik_.z == ik_.w, p == q), res, jab);
             } else {
                 store_dpds(Q.out + __ldg(&Q.mol_out[ch.w]), __ldg(&Q.pairs.info[p]), __ldg(&Q.pairs.info[q]),
                             p == q, res);
             }
         }
+        }
+        if constexpr (JK) {
+            // one addition per J_ab and chunk
+            const int4 ib_ = __ldg(&Q.pairs.info[p]);
+#pragma unroll
+            for (int x = 0; x < 18; ++x) {
+                double v = jab[x];
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+                if (lane == 0) atomicAdd(&Q.jk.J[(long long)(ib_.z + x / 3) * Q.jk.n + ib_.w + x % 3], 2.0 * v);
+            }
         }
     }
 }

@@ -2149,17 +2149,249 @@ __device__ __forceinline__ void store_fppp(double *__restrict__ out, const int4 
       if ((!dcd || 2 >= 2) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[269]; }
 }
 
-// The quartet's unique integrals digested into J and K (molints_plan_jk) instead of stored.
-__device__ __noinline__ void jk_fppp(const JKOut &jk, const int4 ib_, const int4 ik_, bool same,
-                                      const double *__restrict__ res) {
-    const bool dab = ib_.z == ib_.w, dcd = ik_.z == ik_.w;
-    for (int x = 0; x < 270; ++x) {
-        const int ia = x / 27, ibb = (x / 9) % 3, ic = (x / 3) % 3, id = x % 3;
-        if ((dab && ia < ibb) || (dcd && ic < id)) continue;
-        const int i = ib_.z + ia, j = ib_.w + ibb, k = ik_.z + ic, l = ik_.w + id;
-        if (same && pair_index(i, j) < pair_index(k, l)) continue;
-        jk_add(jk, i, j, k, l, res[x]);
+// The quartet's share of J and K (molints_plan_jk, eri_common.cuh): every integral of the block,
+// times f, into one orientation of each target; J_ab stays in the lane (one bra pair per chunk).
+__device__ __forceinline__ void jk_fppp(const JKOut &jk, const int4 ib_, const int4 ik_, double f,
+                                         const double *__restrict__ res, double *__restrict__ jab) {
+    const long long n = jk.n;
+    const double *__restrict__ D = jk.D;
+    const double *__restrict__ Db = D + ib_.w * n, *__restrict__ Dc = D + ik_.z * n;
+    double dcd[9], dbc[9], dbd[9], jcd[9], kbc[9], kbd[9];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int l = 0; l < 3; ++l) {
+            dcd[k * 3 + l] = __ldg(&Dc[k * n + ik_.w + l]);
+            jcd[k * 3 + l] = 0.0;
+        }
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            dbc[j * 3 + k] = __ldg(&Db[j * n + ik_.z + k]);
+            kbc[j * 3 + k] = 0.0;
+        }
+#pragma unroll
+        for (int l = 0; l < 3; ++l) {
+            dbd[j * 3 + l] = __ldg(&Db[j * n + ik_.w + l]);
+            kbd[j * 3 + l] = 0.0;
+        }
     }
+#pragma unroll 1
+    for (int i = 0; i < 10; ++i) {
+        const double *__restrict__ Da = D + (ib_.z + i) * n;
+        double dab[3], dac[3], dad[3], kac[3], kad[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) dab[j] = __ldg(&Da[ib_.w + j]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) { dac[k] = __ldg(&Da[ik_.z + k]); kac[k] = 0.0; }
+#pragma unroll
+        for (int l = 0; l < 3; ++l) { dad[l] = __ldg(&Da[ik_.w + l]); kad[l] = 0.0; }
+        { const double v = f * res[(i * 3 + 0) * 9 + 0];
+          jab[i * 3 + 0] = fma(dcd[0], v, jab[i * 3 + 0]);
+          jcd[0] = fma(dab[0], v, jcd[0]);
+          kac[0] = fma(dbd[0], v, kac[0]);
+          kad[0] = fma(dbc[0], v, kad[0]);
+          kbc[0] = fma(dad[0], v, kbc[0]);
+          kbd[0] = fma(dac[0], v, kbd[0]); }
+        { const double v = f * res[(i * 3 + 0) * 9 + 1];
+          jab[i * 3 + 0] = fma(dcd[1], v, jab[i * 3 + 0]);
+          jcd[1] = fma(dab[0], v, jcd[1]);
+          kac[0] = fma(dbd[1], v, kac[0]);
+          kad[1] = fma(dbc[0], v, kad[1]);
+          kbc[0] = fma(dad[1], v, kbc[0]);
+          kbd[1] = fma(dac[0], v, kbd[1]); }
+        { const double v = f * res[(i * 3 + 0) * 9 + 2];
+          jab[i * 3 + 0] = fma(dcd[2], v, jab[i * 3 + 0]);
+          jcd[2] = fma(dab[0], v, jcd[2]);
+          kac[0] = fma(dbd[2], v, kac[0]);
+          kad[2] = fma(dbc[0], v, kad[2]);
+          kbc[0] = fma(dad[2], v, kbc[0]);
+          kbd[2] = fma(dac[0], v, kbd[2]); }
+        { const double v = f * res[(i * 3 + 0) * 9 + 3];
+          jab[i * 3 + 0] = fma(dcd[3], v, jab[i * 3 + 0]);
+          jcd[3] = fma(dab[0], v, jcd[3]);
+          kac[1] = fma(dbd[0], v, kac[1]);
+          kad[0] = fma(dbc[1], v, kad[0]);
+          kbc[1] = fma(dad[0], v, kbc[1]);
+          kbd[0] = fma(dac[1], v, kbd[0]); }
+        { const double v = f * res[(i * 3 + 0) * 9 + 4];
+          jab[i * 3 + 0] = fma(dcd[4], v, jab[i * 3 + 0]);
+          jcd[4] = fma(dab[0], v, jcd[4]);
+          kac[1] = fma(dbd[1], v, kac[1]);
+          kad[1] = fma(dbc[1], v, kad[1]);
+          kbc[1] = fma(dad[1], v, kbc[1]);
+          kbd[1] = fma(dac[1], v, kbd[1]); }
+        { const double v = f * res[(i * 3 + 0) * 9 + 5];
+          jab[i * 3 + 0] = fma(dcd[5], v, jab[i * 3 + 0]);
+          jcd[5] = fma(dab[0], v, jcd[5]);
+          kac[1] = fma(dbd[2], v, kac[1]);
+          kad[2] = fma(dbc[1], v, kad[2]);
+          kbc[1] = fma(dad[2], v, kbc[1]);
+          kbd[2] = fma(dac[1], v, kbd[2]); }
+        { const double v = f * res[(i * 3 + 0) * 9 + 6];
+          jab[i * 3 + 0] = fma(dcd[6], v, jab[i * 3 + 0]);
+          jcd[6] = fma(dab[0], v, jcd[6]);
+          kac[2] = fma(dbd[0], v, kac[2]);
+          kad[0] = fma(dbc[2], v, kad[0]);
+          kbc[2] = fma(dad[0], v, kbc[2]);
+          kbd[0] = fma(dac[2], v, kbd[0]); }
+        { const double v = f * res[(i * 3 + 0) * 9 + 7];
+          jab[i * 3 + 0] = fma(dcd[7], v, jab[i * 3 + 0]);
+          jcd[7] = fma(dab[0], v, jcd[7]);
+          kac[2] = fma(dbd[1], v, kac[2]);
+          kad[1] = fma(dbc[2], v, kad[1]);
+          kbc[2] = fma(dad[1], v, kbc[2]);
+          kbd[1] = fma(dac[2], v, kbd[1]); }
+        { const double v = f * res[(i * 3 + 0) * 9 + 8];
+          jab[i * 3 + 0] = fma(dcd[8], v, jab[i * 3 + 0]);
+          jcd[8] = fma(dab[0], v, jcd[8]);
+          kac[2] = fma(dbd[2], v, kac[2]);
+          kad[2] = fma(dbc[2], v, kad[2]);
+          kbc[2] = fma(dad[2], v, kbc[2]);
+          kbd[2] = fma(dac[2], v, kbd[2]); }
+        { const double v = f * res[(i * 3 + 1) * 9 + 0];
+          jab[i * 3 + 1] = fma(dcd[0], v, jab[i * 3 + 1]);
+          jcd[0] = fma(dab[1], v, jcd[0]);
+          kac[0] = fma(dbd[3], v, kac[0]);
+          kad[0] = fma(dbc[3], v, kad[0]);
+          kbc[3] = fma(dad[0], v, kbc[3]);
+          kbd[3] = fma(dac[0], v, kbd[3]); }
+        { const double v = f * res[(i * 3 + 1) * 9 + 1];
+          jab[i * 3 + 1] = fma(dcd[1], v, jab[i * 3 + 1]);
+          jcd[1] = fma(dab[1], v, jcd[1]);
+          kac[0] = fma(dbd[4], v, kac[0]);
+          kad[1] = fma(dbc[3], v, kad[1]);
+          kbc[3] = fma(dad[1], v, kbc[3]);
+          kbd[4] = fma(dac[0], v, kbd[4]); }
+        { const double v = f * res[(i * 3 + 1) * 9 + 2];
+          jab[i * 3 + 1] = fma(dcd[2], v, jab[i * 3 + 1]);
+          jcd[2] = fma(dab[1], v, jcd[2]);
+          kac[0] = fma(dbd[5], v, kac[0]);
+          kad[2] = fma(dbc[3], v, kad[2]);
+          kbc[3] = fma(dad[2], v, kbc[3]);
+          kbd[5] = fma(dac[0], v, kbd[5]); }
+        { const double v = f * res[(i * 3 + 1) * 9 + 3];
+          jab[i * 3 + 1] = fma(dcd[3], v, jab[i * 3 + 1]);
+          jcd[3] = fma(dab[1], v, jcd[3]);
+          kac[1] = fma(dbd[3], v, kac[1]);
+          kad[0] = fma(dbc[4], v, kad[0]);
+          kbc[4] = fma(dad[0], v, kbc[4]);
+          kbd[3] = fma(dac[1], v, kbd[3]); }
+        { const double v = f * res[(i * 3 + 1) * 9 + 4];
+          jab[i * 3 + 1] = fma(dcd[4], v, jab[i * 3 + 1]);
+          jcd[4] = fma(dab[1], v, jcd[4]);
+          kac[1] = fma(dbd[4], v, kac[1]);
+          kad[1] = fma(dbc[4], v, kad[1]);
+          kbc[4] = fma(dad[1], v, kbc[4]);
+          kbd[4] = fma(dac[1], v, kbd[4]); }
+        { const double v = f * res[(i * 3 + 1) * 9 + 5];
+          jab[i * 3 + 1] = fma(dcd[5], v, jab[i * 3 + 1]);
+          jcd[5] = fma(dab[1], v, jcd[5]);
+          kac[1] = fma(dbd[5], v, kac[1]);
+          kad[2] = fma(dbc[4], v, kad[2]);
+          kbc[4] = fma(dad[2], v, kbc[4]);
+          kbd[5] = fma(dac[1], v, kbd[5]); }
+        { const double v = f * res[(i * 3 + 1) * 9 + 6];
+          jab[i * 3 + 1] = fma(dcd[6], v, jab[i * 3 + 1]);
+          jcd[6] = fma(dab[1], v, jcd[6]);
+          kac[2] = fma(dbd[3], v, kac[2]);
+          kad[0] = fma(dbc[5], v, kad[0]);
+          kbc[5] = fma(dad[0], v, kbc[5]);
+          kbd[3] = fma(dac[2], v, kbd[3]); }
+        { const double v = f * res[(i * 3 + 1) * 9 + 7];
+          jab[i * 3 + 1] = fma(dcd[7], v, jab[i * 3 + 1]);
+          jcd[7] = fma(dab[1], v, jcd[7]);
+          kac[2] = fma(dbd[4], v, kac[2]);
+          kad[1] = fma(dbc[5], v, kad[1]);
+          kbc[5] = fma(dad[1], v, kbc[5]);
+          kbd[4] = fma(dac[2], v, kbd[4]); }
+        { const double v = f * res[(i * 3 + 1) * 9 + 8];
+          jab[i * 3 + 1] = fma(dcd[8], v, jab[i * 3 + 1]);
+          jcd[8] = fma(dab[1], v, jcd[8]);
+          kac[2] = fma(dbd[5], v, kac[2]);
+          kad[2] = fma(dbc[5], v, kad[2]);
+          kbc[5] = fma(dad[2], v, kbc[5]);
+          kbd[5] = fma(dac[2], v, kbd[5]); }
+        { const double v = f * res[(i * 3 + 2) * 9 + 0];
+          jab[i * 3 + 2] = fma(dcd[0], v, jab[i * 3 + 2]);
+          jcd[0] = fma(dab[2], v, jcd[0]);
+          kac[0] = fma(dbd[6], v, kac[0]);
+          kad[0] = fma(dbc[6], v, kad[0]);
+          kbc[6] = fma(dad[0], v, kbc[6]);
+          kbd[6] = fma(dac[0], v, kbd[6]); }
+        { const double v = f * res[(i * 3 + 2) * 9 + 1];
+          jab[i * 3 + 2] = fma(dcd[1], v, jab[i * 3 + 2]);
+          jcd[1] = fma(dab[2], v, jcd[1]);
+          kac[0] = fma(dbd[7], v, kac[0]);
+          kad[1] = fma(dbc[6], v, kad[1]);
+          kbc[6] = fma(dad[1], v, kbc[6]);
+          kbd[7] = fma(dac[0], v, kbd[7]); }
+        { const double v = f * res[(i * 3 + 2) * 9 + 2];
+          jab[i * 3 + 2] = fma(dcd[2], v, jab[i * 3 + 2]);
+          jcd[2] = fma(dab[2], v, jcd[2]);
+          kac[0] = fma(dbd[8], v, kac[0]);
+          kad[2] = fma(dbc[6], v, kad[2]);
+          kbc[6] = fma(dad[2], v, kbc[6]);
+          kbd[8] = fma(dac[0], v, kbd[8]); }
+        { const double v = f * res[(i * 3 + 2) * 9 + 3];
+          jab[i * 3 + 2] = fma(dcd[3], v, jab[i * 3 + 2]);
+          jcd[3] = fma(dab[2], v, jcd[3]);
+          kac[1] = fma(dbd[6], v, kac[1]);
+          kad[0] = fma(dbc[7], v, kad[0]);
+          kbc[7] = fma(dad[0], v, kbc[7]);
+          kbd[6] = fma(dac[1], v, kbd[6]); }
+        { const double v = f * res[(i * 3 + 2) * 9 + 4];
+          jab[i * 3 + 2] = fma(dcd[4], v, jab[i * 3 + 2]);
+          jcd[4] = fma(dab[2], v, jcd[4]);
+          kac[1] = fma(dbd[7], v, kac[1]);
+          kad[1] = fma(dbc[7], v, kad[1]);
+          kbc[7] = fma(dad[1], v, kbc[7]);
+          kbd[7] = fma(dac[1], v, kbd[7]); }
+        { const double v = f * res[(i * 3 + 2) * 9 + 5];
+          jab[i * 3 + 2] = fma(dcd[5], v, jab[i * 3 + 2]);
+          jcd[5] = fma(dab[2], v, jcd[5]);
+          kac[1] = fma(dbd[8], v, kac[1]);
+          kad[2] = fma(dbc[7], v, kad[2]);
+          kbc[7] = fma(dad[2], v, kbc[7]);
+          kbd[8] = fma(dac[1], v, kbd[8]); }
+        { const double v = f * res[(i * 3 + 2) * 9 + 6];
+          jab[i * 3 + 2] = fma(dcd[6], v, jab[i * 3 + 2]);
+          jcd[6] = fma(dab[2], v, jcd[6]);
+          kac[2] = fma(dbd[6], v, kac[2]);
+          kad[0] = fma(dbc[8], v, kad[0]);
+          kbc[8] = fma(dad[0], v, kbc[8]);
+          kbd[6] = fma(dac[2], v, kbd[6]); }
+        { const double v = f * res[(i * 3 + 2) * 9 + 7];
+          jab[i * 3 + 2] = fma(dcd[7], v, jab[i * 3 + 2]);
+          jcd[7] = fma(dab[2], v, jcd[7]);
+          kac[2] = fma(dbd[7], v, kac[2]);
+          kad[1] = fma(dbc[8], v, kad[1]);
+          kbc[8] = fma(dad[1], v, kbc[8]);
+          kbd[7] = fma(dac[2], v, kbd[7]); }
+        { const double v = f * res[(i * 3 + 2) * 9 + 8];
+          jab[i * 3 + 2] = fma(dcd[8], v, jab[i * 3 + 2]);
+          jcd[8] = fma(dab[2], v, jcd[8]);
+          kac[2] = fma(dbd[8], v, kac[2]);
+          kad[2] = fma(dbc[8], v, kad[2]);
+          kbc[8] = fma(dad[2], v, kbc[8]);
+          kbd[8] = fma(dac[2], v, kbd[8]); }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) atomicAdd(&jk.K[(ib_.z + i) * n + ik_.z + k], kac[k]);
+#pragma unroll
+        for (int l = 0; l < 3; ++l) atomicAdd(&jk.K[(ib_.z + i) * n + ik_.w + l], kad[l]);
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) atomicAdd(&jk.K[(ib_.w + j) * n + ik_.z + k], kbc[j * 3 + k]);
+#pragma unroll
+        for (int l = 0; l < 3; ++l) atomicAdd(&jk.K[(ib_.w + j) * n + ik_.w + l], kbd[j * 3 + l]);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int l = 0; l < 3; ++l) atomicAdd(&jk.J[(ik_.z + k) * n + ik_.w + l], 2.0 * jcd[k * 3 + l]);
 }
 
 // Persistent work-queue kernel: each warp takes chunks (one bra pair, a run of consecutive
@@ -2185,6 +2417,11 @@ __global__ void __launch_bounds__(128) eri_queue_fppp(const EriQueue Q) {
         const int p = ch.x, cnt = ch.z & 0xffff, lg = (ch.z >> 16) & 7, lgj = (ch.z >> 20) & 7;
         const int W = 32 >> lg, kq = lane & (W - 1), s = lane >> (5 - lg);
         const int js = s & ((1 << lgj) - 1), is = s >> lgj;
+        double jab[JK ? 30 : 1];  // J/K digestion: the bra pair's J, over the chunk
+        if constexpr (JK) {
+#pragma unroll
+            for (int x = 0; x < 30; ++x) jab[x] = 0.0;
+        }
         for (int base = 0; base < cnt; base += W) {
         const int q = ch.y + base + kq;
         const bool live = base + kq < cnt;
@@ -2224,12 +2461,24 @@ __global__ void __launch_bounds__(128) eri_queue_fppp(const EriQueue Q) {
             double res[270];
             hrr_fppp(Q.pairs, p, q, acc, res);
             if constexpr (JK) {
-                jk_fppp(Q.jk, __ldg(&Q.pairs.info[p]), __ldg(&Q.pairs.info[q]), p == q, res);
+                const int4 ib_ = __ldg(&Q.pairs.info[p]), ik_ = __ldg(&Q.pairs.info[q]);
+                jk_fppp(Q.jk, ib_, ik_, jk_weight(ib_.z == ib_.w, ik_.z == ik_.w, p == q), res, jab);
             } else {
                 store_fppp(Q.out + __ldg(&Q.mol_out[ch.w]), __ldg(&Q.pairs.info[p]), __ldg(&Q.pairs.info[q]),
                             p == q, res);
             }
         }
+        }
+        if constexpr (JK) {
+            // one addition per J_ab and chunk
+            const int4 ib_ = __ldg(&Q.pairs.info[p]);
+#pragma unroll
+            for (int x = 0; x < 30; ++x) {
+                double v = jab[x];
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+                if (lane == 0) atomicAdd(&Q.jk.J[(long long)(ib_.z + x / 3) * Q.jk.n + ib_.w + x % 3], 2.0 * v);
+            }
         }
     }
 }

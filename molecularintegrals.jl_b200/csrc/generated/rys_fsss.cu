@@ -125,17 +125,67 @@ __device__ __forceinline__ void store_fsss_rys(double *__restrict__ out, const i
       if ((!dcd || 0 >= 0) && (!same || ij >= kl)) out[packed_index(ij, kl)] = res[9]; }
 }
 
-// The quartet's unique integrals digested into J and K (molints_plan_jk) instead of stored.
-__device__ __noinline__ void jk_fsss_rys(const JKOut &jk, const int4 ib_, const int4 ik_, bool same,
-                                      const double *__restrict__ res) {
-    const bool dab = ib_.z == ib_.w, dcd = ik_.z == ik_.w;
-    for (int x = 0; x < 10; ++x) {
-        const int ia = x / 1, ibb = (x / 1) % 1, ic = (x / 1) % 1, id = x % 1;
-        if ((dab && ia < ibb) || (dcd && ic < id)) continue;
-        const int i = ib_.z + ia, j = ib_.w + ibb, k = ik_.z + ic, l = ik_.w + id;
-        if (same && pair_index(i, j) < pair_index(k, l)) continue;
-        jk_add(jk, i, j, k, l, res[x]);
+// The quartet's share of J and K (molints_plan_jk, eri_common.cuh): every integral of the block,
+// times f, into one orientation of each target; J_ab stays in the lane (one bra pair per chunk).
+__device__ __forceinline__ void jk_fsss_rys(const JKOut &jk, const int4 ib_, const int4 ik_, double f,
+                                         const double *__restrict__ res, double *__restrict__ jab) {
+    const long long n = jk.n;
+    const double *__restrict__ D = jk.D;
+    const double *__restrict__ Db = D + ib_.w * n, *__restrict__ Dc = D + ik_.z * n;
+    double dcd[1], dbc[1], dbd[1], jcd[1], kbc[1], kbd[1];
+#pragma unroll
+    for (int k = 0; k < 1; ++k)
+#pragma unroll
+        for (int l = 0; l < 1; ++l) {
+            dcd[k * 1 + l] = __ldg(&Dc[k * n + ik_.w + l]);
+            jcd[k * 1 + l] = 0.0;
+        }
+#pragma unroll
+    for (int j = 0; j < 1; ++j) {
+#pragma unroll
+        for (int k = 0; k < 1; ++k) {
+            dbc[j * 1 + k] = __ldg(&Db[j * n + ik_.z + k]);
+            kbc[j * 1 + k] = 0.0;
+        }
+#pragma unroll
+        for (int l = 0; l < 1; ++l) {
+            dbd[j * 1 + l] = __ldg(&Db[j * n + ik_.w + l]);
+            kbd[j * 1 + l] = 0.0;
+        }
     }
+#pragma unroll 10
+    for (int i = 0; i < 10; ++i) {
+        const double *__restrict__ Da = D + (ib_.z + i) * n;
+        double dab[1], dac[1], dad[1], kac[1], kad[1];
+#pragma unroll
+        for (int j = 0; j < 1; ++j) dab[j] = __ldg(&Da[ib_.w + j]);
+#pragma unroll
+        for (int k = 0; k < 1; ++k) { dac[k] = __ldg(&Da[ik_.z + k]); kac[k] = 0.0; }
+#pragma unroll
+        for (int l = 0; l < 1; ++l) { dad[l] = __ldg(&Da[ik_.w + l]); kad[l] = 0.0; }
+        { const double v = f * res[(i * 1 + 0) * 1 + 0];
+          jab[i * 1 + 0] = fma(dcd[0], v, jab[i * 1 + 0]);
+          jcd[0] = fma(dab[0], v, jcd[0]);
+          kac[0] = fma(dbd[0], v, kac[0]);
+          kad[0] = fma(dbc[0], v, kad[0]);
+          kbc[0] = fma(dad[0], v, kbc[0]);
+          kbd[0] = fma(dac[0], v, kbd[0]); }
+#pragma unroll
+        for (int k = 0; k < 1; ++k) atomicAdd(&jk.K[(ib_.z + i) * n + ik_.z + k], kac[k]);
+#pragma unroll
+        for (int l = 0; l < 1; ++l) atomicAdd(&jk.K[(ib_.z + i) * n + ik_.w + l], kad[l]);
+    }
+#pragma unroll
+    for (int j = 0; j < 1; ++j) {
+#pragma unroll
+        for (int k = 0; k < 1; ++k) atomicAdd(&jk.K[(ib_.w + j) * n + ik_.z + k], kbc[j * 1 + k]);
+#pragma unroll
+        for (int l = 0; l < 1; ++l) atomicAdd(&jk.K[(ib_.w + j) * n + ik_.w + l], kbd[j * 1 + l]);
+    }
+#pragma unroll
+    for (int k = 0; k < 1; ++k)
+#pragma unroll
+        for (int l = 0; l < 1; ++l) atomicAdd(&jk.J[(ik_.z + k) * n + ik_.w + l], 2.0 * jcd[k * 1 + l]);
 }
 
 // Persistent work-queue kernel: each warp takes chunks (one bra pair, a run of consecutive
@@ -161,6 +211,11 @@ __global__ void __launch_bounds__(128) eri_queue_fsss_rys(const EriQueue Q) {
         const int p = ch.x, cnt = ch.z & 0xffff, lg = (ch.z >> 16) & 7, lgj = (ch.z >> 20) & 7;
         const int W = 32 >> lg, kq = lane & (W - 1), s = lane >> (5 - lg);
         const int js = s & ((1 << lgj) - 1), is = s >> lgj;
+        double jab[JK ? 10 : 1];  // J/K digestion: the bra pair's J, over the chunk
+        if constexpr (JK) {
+#pragma unroll
+            for (int x = 0; x < 10; ++x) jab[x] = 0.0;
+        }
         for (int base = 0; base < cnt; base += W) {
         const int q = ch.y + base + kq;
         const bool live = base + kq < cnt;
@@ -201,12 +256,24 @@ __global__ void __launch_bounds__(128) eri_queue_fsss_rys(const EriQueue Q) {
             double res[10];
             hrr_fsss_rys(Q.pairs, p, q, acc, res);
             if constexpr (JK) {
-                jk_fsss_rys(Q.jk, __ldg(&Q.pairs.info[p]), __ldg(&Q.pairs.info[q]), p == q, res);
+                const int4 ib_ = __ldg(&Q.pairs.info[p]), ik_ = __ldg(&Q.pairs.info[q]);
+                jk_fsss_rys(Q.jk, ib_, ik_, jk_weight(ib_.z == ib_.w, ik_.z == ik_.w, p == q), res, jab);
             } else {
                 store_fsss_rys(Q.out + __ldg(&Q.mol_out[ch.w]), __ldg(&Q.pairs.info[p]), __ldg(&Q.pairs.info[q]),
                             p == q, res);
             }
         }
+        }
+        if constexpr (JK) {
+            // one addition per J_ab and chunk
+            const int4 ib_ = __ldg(&Q.pairs.info[p]);
+#pragma unroll
+            for (int x = 0; x < 10; ++x) {
+                double v = jab[x];
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+                if (lane == 0) atomicAdd(&Q.jk.J[(long long)(ib_.z + x / 1) * Q.jk.n + ib_.w + x % 1], 2.0 * v);
+            }
         }
     }
 }

@@ -597,15 +597,16 @@ __global__ void __launch_bounds__(kGatherThreads) gather_packed_kernel(
     }
 }
 
-// Copy the lower triangles of J and K (the digestion accumulates only those) to the upper.
-__global__ void mirror_lower_kernel(double *__restrict__ J, double *__restrict__ K, int n) {
+// J = X + X^T and K = Y + Y^T in place (the digestion accumulates one orientation of each target).
+__global__ void add_transpose_kernel(double *__restrict__ J, double *__restrict__ K, int n) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)n * n) return;
     const int r = (int)(t / n), c = (int)(t - (long long)r * n);
-    if (r < c) {
-        J[(long long)r * n + c] = J[(long long)c * n + r];
-        K[(long long)r * n + c] = K[(long long)c * n + r];
-    }
+    if (r > c) return;
+    const long long u = (long long)c * n + r;
+    const double j = J[t] + J[u], k = K[t] + K[u];
+    J[t] = J[u] = j;
+    K[t] = K[u] = k;
 }
 
 __global__ void boys_eval_kernel(BoysTab bt, int mmax, const double *__restrict__ T, long long n,
@@ -2032,9 +2033,9 @@ int molints_plan_jk(molints_plan *p, const double *D_device, double *J_device, d
     jk.n = (int)n;
     const int rc = plan_enqueue(p, nullptr, true, jk);
     if (rc) return rc;
-    if (n > 1) {
+    if (n > 0) {
         const long long nn = (long long)n * n;
-        mirror_lower_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, ctx->stream>>>(J_device, K_device, (int)n);
+        add_transpose_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, ctx->stream>>>(J_device, K_device, (int)n);
         MI_CUDA(ctx, cudaGetLastError());
     }
     return MOLINTS_OK;

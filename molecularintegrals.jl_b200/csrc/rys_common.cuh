@@ -280,6 +280,68 @@ __device__ __forceinline__ double *rys_hrr(const PairTab &P, const RysClassTabs 
     return stg;
 }
 
+// The round's quartets into J and K (jk_weight, eri_common.cuh): a thread per target (J_ab, J_cd,
+// K_ac, K_ad, K_bc, K_bd) sums its terms of the block in shared memory and adds once.
+template <class C>
+__device__ __noinline__ void rys_digest(const JKOut jk, const int4 *__restrict__ info, const int4 ib, int p, int q0,
+                                        int nlive, const double *__restrict__ stg, int lane) {
+    constexpr int NB = C::NB, ND = C::ND, NA1 = C::NAB / NB, NC1 = C::NCD / ND;
+    constexpr int T0 = C::NAB, T1 = T0 + C::NCD, T2 = T1 + NA1 * NC1, T3 = T2 + NA1 * ND, T4 = T3 + NB * NC1,
+                  T5 = T4 + NB * ND;
+    const double *__restrict__ D = jk.D;
+    const long long n = jk.n;
+    for (int t = lane; t < nlive * T5; t += C::G) {
+        const int w = t / T5, k = t - w * T5;
+        const int4 ik = __ldg(&info[q0 + w]);
+        const double f = jk_weight(ib.z == ib.w, ik.z == ik.w, p == q0 + w);
+        const double *__restrict__ v = stg + w * C::NAB * C::NCDP;  // v[(a NB + b) NCDP + c ND + d]
+        double s = 0.0;
+        if (k < T0) {
+            const int a = k / NB, b = k - a * NB;
+            for (int c = 0; c < NC1; ++c)
+#pragma unroll
+                for (int d = 0; d < ND; ++d)
+                    s = fma(__ldg(&D[(ik.z + c) * n + ik.w + d]), v[k * C::NCDP + c * ND + d], s);
+            atomicAdd(&jk.J[(ib.z + a) * n + ib.w + b], 2.0 * f * s);
+        } else if (k < T1) {
+            const int x = k - T0, c = x / ND, d = x - c * ND;
+            for (int a = 0; a < NA1; ++a)
+#pragma unroll
+                for (int b = 0; b < NB; ++b)
+                    s = fma(__ldg(&D[(ib.z + a) * n + ib.w + b]), v[(a * NB + b) * C::NCDP + x], s);
+            atomicAdd(&jk.J[(ik.z + c) * n + ik.w + d], 2.0 * f * s);
+        } else if (k < T2) {
+            const int x = k - T1, a = x / NC1, c = x - a * NC1;
+            for (int b = 0; b < NB; ++b)
+#pragma unroll
+                for (int d = 0; d < ND; ++d)
+                    s = fma(__ldg(&D[(ib.w + b) * n + ik.w + d]), v[(a * NB + b) * C::NCDP + c * ND + d], s);
+            atomicAdd(&jk.K[(ib.z + a) * n + ik.z + c], f * s);
+        } else if (k < T3) {
+            const int x = k - T2, a = x / ND, d = x - a * ND;
+            for (int b = 0; b < NB; ++b)
+#pragma unroll
+                for (int c = 0; c < NC1; ++c)
+                    s = fma(__ldg(&D[(ib.w + b) * n + ik.z + c]), v[(a * NB + b) * C::NCDP + c * ND + d], s);
+            atomicAdd(&jk.K[(ib.z + a) * n + ik.w + d], f * s);
+        } else if (k < T4) {
+            const int x = k - T3, b = x / NC1, c = x - b * NC1;
+            for (int a = 0; a < NA1; ++a)
+#pragma unroll
+                for (int d = 0; d < ND; ++d)
+                    s = fma(__ldg(&D[(ib.z + a) * n + ik.w + d]), v[(a * NB + b) * C::NCDP + c * ND + d], s);
+            atomicAdd(&jk.K[(ib.w + b) * n + ik.z + c], f * s);
+        } else {
+            const int x = k - T4, b = x / ND, d = x - b * ND;
+            for (int a = 0; a < NA1; ++a)
+#pragma unroll
+                for (int c = 0; c < NC1; ++c)
+                    s = fma(__ldg(&D[(ib.z + a) * n + ik.z + c]), v[(a * NB + b) * C::NCDP + c * ND + d], s);
+            atomicAdd(&jk.K[(ib.w + b) * n + ik.w + d], f * s);
+        }
+    }
+}
+
 // Persistent work-queue kernel body: each group takes chunks (one bra pair, a run of ket pairs
 // of one molecule) from the class pair's counter and computes their quartets W at a time.
 template <class C, int MIXED = 0>
@@ -346,6 +408,8 @@ __device__ __forceinline__ void rys_queue_body(const EriQueue &Q, const RysTab &
                     const int row = x / NCD;
                     dst[x] = stg[row * C::NCDP + (x - row * NCD)];
                 }
+            } else if (Q.jk.J) {
+                rys_digest<C>(Q.jk, Q.pairs.info, ib, p, q0, nlive, stg, lane);
             } else {
                 double *__restrict__ out = Q.out + __ldg(&Q.mol_out[ch.w]);
                 const bool dab = ib.z == ib.w;
@@ -356,9 +420,7 @@ __device__ __forceinline__ void rys_queue_body(const EriQueue &Q, const RysTab &
                     if ((dab && ia < jb) || (ik.z == ik.w && ic < jd)) continue;
                     const long long ij = pair_index(ib.z + ia, ib.w + jb), kl = pair_index(ik.z + ic, ik.w + jd);
                     if (p == q0 + w && ij < kl) continue;
-                    const double v = stg[row * C::NCDP + s];
-                    if (Q.jk.J) jk_add(Q.jk, ib.z + ia, ib.w + jb, ik.z + ic, ik.w + jd, v);
-                    else out[packed_index(ij, kl)] = v;
+                    out[packed_index(ij, kl)] = stg[row * C::NCDP + s];
                 }
             }
             group_sync<C::G>(gid);
