@@ -179,7 +179,7 @@ int molints_get_class_methods(const molints_ctx *ctx, int32_t *methods, int32_t 
  * reference evaluates one shell quartet at a time).  Plans created after the call use it.
  *   lane_cost     HGP lane split: a quartet's primitive quartets are spread over up to 32
  *                 lanes until one lane's share costs at most lane_cost (ss|ss)-equivalents
- *                 (default 80)
+ *                 (default 80); quartets of small molecules are split finer, down to 30
  *   hgp_widen     ket pairs of an unsplit HGP chunk, in units of 32 (one per lane) (default 1;
  *                 very large batches widen further to bound the queue length)
  *   rys_chunks    Rys chunks are as long as keeps about this many chunks in a class queue

@@ -55,8 +55,13 @@ struct molints_ctx {
     cudaEvent_t scratch_ev = nullptr;
     bool scratch_ev_live = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    // class-pair kernels run concurrently on side streams forked from `stream`
-    static constexpr int kSide = 6;
+    // Class-pair kernels run concurrently on side streams forked from `stream`.  Direct plans (small
+    // ones among them: 22 to 57 kernels of 10-40 us that fill a few SMs each) take up to kSide;
+    // two-phase plans, whose kernels fill the device and share L2 with the scratch they write, take
+    // kSideTwoPhase.  On B200, us per execute with 6 / 16 / 24 streams: 8 polarised atoms 99 / 87 /
+    // 78, 11 atoms with f shells 340 / 277 / 254, 15 polarised atoms 324 / 329 / 335, a batch of
+    // 1.17e9 integrals 7025 / 7139 / 7253.
+    static constexpr int kSide = 24, kSideTwoPhase = 6;
     cudaStream_t side[kSide] = {};
     cudaEvent_t fork = nullptr, join[kSide] = {};
     int num_sms = 0;
@@ -1366,7 +1371,6 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
         for (int c = 0; c <= kNumPairClasses; ++c) S.cls_start[c] = cls_start[c];
         S.nmol = nmol;
         S.widen = hgp_widen;
-        S.lane_cost = ctx->sched.lane_cost;
         p->gather_blocks = ctx->sched.gather_blocks;
         S.sharded = sharded;
         S.shard_s0 = shard_s0;
@@ -1451,7 +1455,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     Carve tv;
     const size_t t_ab1 = tv.take<int2>(npair), t_info1 = tv.take<int4>(npair), t_rec1 = tv.take<int4>(npair);
     const size_t t_seg1 = tv.take<int>(npair), t_mol1 = tv.take<int>(npair);
-    const size_t t_cm = tv.take<int>(cm_start.size());
+    const size_t t_cm = tv.take<int>(cm_start.size()), t_lane = tv.take<double>(nmol);
     const size_t up_bytes = tv.at;
     const size_t t_src1 = tv.take<int>(nall);
     const size_t t_pbound = tv.take<double2>(nall), t_qmax = tv.take<unsigned long long>(nmol);
@@ -1500,6 +1504,10 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
             mol1[k] = m;
         }
         std::memcpy(up + t_cm, cm_start.data(), cm_start.size() * sizeof(int));
+        double *lane = reinterpret_cast<double *>(up + t_lane);
+        for (int m = 0; m < nmol; ++m) lane[m] = 0.0;
+        for (const PairRec &r : pr) lane[r.mol] += r.npp;
+        for (int m = 0; m < nmol; ++m) lane[m] = molecule_lane_cost(lane[m], ctx->sched.lane_cost);
     }
     std::memcpy(stage + o_xyz, xyz.data(), 3 * (size_t)ns * sizeof(double));
     std::memcpy(stage + o_expn, expn.data(), (size_t)nprim * sizeof(double));
@@ -1672,6 +1680,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     QA.npp_prefix = A.npp_prefix;
     QA.region = tp ? p->g_region : nullptr;
     QA.bnd = p->bnd;
+    QA.lane_cost = reinterpret_cast<const double *>(tmp + t_lane);
     QA.cnt = reinterpret_cast<long long *>(tmp + t_cnt);
     QA.cost = reinterpret_cast<double *>(tmp + t_cost);
     QA.off = reinterpret_cast<long long *>(tmp + t_off);
@@ -1866,7 +1875,9 @@ static int plan_enqueue(molints_plan *p, double *out_device, bool timing, JKOut 
     std::stable_sort(jobs.begin(), jobs.end(), [](const Job &a, const Job &b) { return a.cost > b.cost; });
     // Profiling runs every launch on the caller's stream, so each event pair times one kernel.
     const int ngen = p->n_gq > 0;
-    const int nside = p->profiling ? 0 : std::min<int>(molints_ctx::kSide, (int)jobs.size() + ngen);
+    const int nside = p->profiling ? 0
+                                   : std::min<int>(p->two_phase ? molints_ctx::kSideTwoPhase : molints_ctx::kSide,
+                                                   (int)jobs.size() + ngen);
     int fp32_launches = 0;
     if (nside > 0) MI_CUDA(ctx, cudaEventRecord(ctx->fork, s));
     for (int i = 0; i < nside; ++i) MI_CUDA(ctx, cudaStreamWaitEvent(ctx->side[i], ctx->fork, 0));

@@ -4,7 +4,7 @@
 //
 // The reference builds its work list on the host, one shell quartet at a time
 // (eri_fetcher, src/Basis.jl:201-262); here the list is chunks of one bra pair and a run of
-// ket pairs, emitted in parallel (one thread per bra pair of each class pair) and ordered by
+// ket pairs, emitted in parallel (a warp per bra pair of each class pair) and ordered by
 // class pair and decreasing cost with a stable radix sort.
 #pragma once
 
@@ -18,6 +18,7 @@ namespace molints {
 
 constexpr int kNumClassPairs = kNumPairClasses * (kNumPairClasses + 1) / 2;  // (x, y <= x)
 constexpr int kCostBuckets = 64;
+constexpr double kLaneCostPerPair = 0.015, kLaneCostMin = 30.0;  // molecule_lane_cost
 
 // Lane split of an HGP work-queue chunk whose bra pair has nb and ket pair nk kept primitive
 // pairs, in a class whose primitive quartet costs `cost` (kEriPrimCost; (ss|ss) ~ 1).  A lane
@@ -39,6 +40,20 @@ __host__ __device__ inline int hgp_split(int nb, int nk, double cost, double lan
         ++lg;
     }
     return lg | (lgj << 4);
+}
+
+// The lane-split bound of a molecule's quartets: the schedule's lane_cost for large molecules, less
+// for small ones.  npp is the molecule's primitive pairs (before screening), npp^2 / 2 the primitive
+// quartets.  A large molecule has work for every lane of the device, and splits only cost it idle
+// lanes and reductions; in a small one the kernels end with their longest lane, so its heavy quartets
+// are split finer, in proportion to the square root of the work.  A function of the molecule, not of
+// the plan: the same quartet gets the same split alone and in a batch.  Measured on B200, us per
+// execute with 640 for every molecule / this: 8 polarised atoms 263 / 99, 9 split-valence atoms
+// 153 / 41, 24 split-valence atoms 307 / 251, 11 atoms with f shells 467 / 340, J/K of 15 polarised
+// atoms 435 / 342, a batch of 1.17e9 integrals 7027 / 7025 (six streams throughout).
+__host__ __device__ inline double molecule_lane_cost(double npp, double lane_cost) {
+    const double c = kLaneCostPerPair * npp;
+    return fmin(lane_cost, fmax(kLaneCostMin, c));
 }
 
 // Cost bucket of a chunk, heaviest first: 0 for the largest binary exponents.  An O(1) key
@@ -114,7 +129,6 @@ struct QueueSetup {
     int cls_start[kNumPairClasses + 1];
     int nmol;
     int widen;                          // HGP chunk widths are (32 >> lg) * widen
-    double lane_cost;
     int sharded, shard_s0, shard_s1;    // shard plans: owned highest-shell range [s0, s1)
     int ps0[kNumPairClasses], ps1[kNumPairClasses];  // first pair of each class with ms >= s0 / s1
     int two_phase;
@@ -189,6 +203,7 @@ struct QueueArgs {
     const long long *npp_prefix;
     const long long *region;       // two-phase: per (x, y, molecule) 4 fields, else null
     const double2 *bnd;            // per final pair (Qabs, R): the screening order's cut
+    const double *lane_cost;       // per molecule: molecule_lane_cost
     long long *cnt;                // n_items + 1
     double *cost;                  // n_items
     long long *off;                // n_items + 1

@@ -1,4 +1,7 @@
-"""CPU test of nonzero_end (csrc/plan_build.cuh): the first pair without kept primitive pairs of a
+"""CPU test of host-callable helpers of the plan build (csrc/plan_build.cuh).
+
+molecule_lane_cost: non-decreasing in the molecule's primitive pairs, never above the schedule's
+bound, the bound itself for large molecules.  nonzero_end: the first pair without kept primitive pairs of a
 run in descending kept count, against a linear scan, for every run of up to 40 pairs and every
 sub-run.  The work queues end each bra's ket run there."""
 import shutil
@@ -27,6 +30,15 @@ int main() {
                     if (nonzero_end(npp.data(), b, e) != want) ++bad;
                 }
         }
+    for (double bound : {5.0, 30.0, 80.0, 640.0, 1e6}) {
+        double prev = 0.0;
+        for (double npp = 0.0; npp < 1e6; npp = npp * 1.3 + 1.0) {
+            const double c = molecule_lane_cost(npp, bound);
+            if (!(c > 0.0) || c < prev || c > bound) ++bad;
+            prev = c;
+        }
+        if (bound <= 1e4 && molecule_lane_cost(1e6, bound) != bound) ++bad;
+    }
     std::printf("%d\n", bad);
     return bad != 0;
 }
