@@ -13,6 +13,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -136,12 +137,13 @@ struct molints_plan {
     long long *g_mol = nullptr;        // per molecule: {first function, first pair entry, packed offset,
                                        // first function-pair entry of g_col}
     int2 *g_col = nullptr;             // per function pair of every molecule: gather_cols_kernel
-    double *g_colq = nullptr;          // beside g_col when quartets are screened: Qabs of its pair
-    double *g_qmax = nullptr;          // per molecule when quartets are screened: a bound of every
-                                       // pair's Qabs (the largest sum of b_k over all its
-                                       // primitive pairs)
+    int4 *g_list = nullptr;            // gather_list_kernel: the columns that are not zero, ...
+    double *g_colq = nullptr;          // ... the Qabs of their pairs (plans that screen quartets),
+    int *g_index = nullptr, *g_end = nullptr;  // and where a molecule's columns are in the list
     int4 *g_units = nullptr;           // gather units: shell pairs, heaviest first (gather_packed_kernel)
+    int *g_nlive = nullptr;            // units with entries (they come first)
     int64_t n_units = 0;
+    int64_t n_rows = 0;                // function pairs of all molecules
     int64_t bytes = 0;
     int n_launches = 0;
     int n_fp32_launches = 0;           // class-pair launches of the last execute that ran FP32
@@ -409,25 +411,34 @@ __device__ __forceinline__ long long untri_f(long long t) {
 }
 
 constexpr int kGatherThreads = 256;
+constexpr int kGatherStretch = 8192;  // entries of a stretch, over P's rows (at least 1024 columns)
 
 // Per function pair (i >= j) of every molecule of a two-phase plan, what the gather needs to
 // place its entries, built once per plan on the device: x = list position << 4 | pair class of
 // the shell pair holding (i, j), or -1 if none of the pair's primitive pairs was kept (its quartets
 // are zero, and in no chunk), y = component of the function in that pair's A << 16 | component in
-// its B; colq (plans that screen quartets) the pair's Qabs.  Entry (m, ij) is at
-// col[mol[4m+3] + ij]; thread r takes entry r, of the molecule m with
-// mol[4m+3] <= r < mol[4(m+1)+3] (the molecules' entries follow one another).
-__global__ void gather_cols_kernel(int2 *__restrict__ col, double *__restrict__ colq,
-                                   const double2 *__restrict__ bnd, const int4 *__restrict__ info,
-                                   const int2 *__restrict__ fn, const int *__restrict__ pairs,
-                                   const long long *__restrict__ mol, int nmol, long long nrows) {
-    const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= nrows) return;
+// its B.  Entry (m, ij) is at col[mol[4m+3] + ij]; thread r takes entry r, of the molecule m with
+// mol[4m+3] <= r < mol[4(m+1)+3] (the molecules' entries follow one another).  nonzero[r]: 1 if x >= 0
+// (its prefix sums place the list of gather_list_kernel; entry nrows is 0).
+__device__ __forceinline__ int gather_mol_of(const long long *__restrict__ mol, int nmol, long long r) {
     int m = 0, hi = nmol;  // last m with mol[4m+3] <= r
     while (hi - m > 1) {
         const int mid = (m + hi) >> 1;
         if (__ldg(&mol[4 * mid + 3]) <= r) m = mid; else hi = mid;
     }
+    return m;
+}
+
+__global__ void gather_cols_kernel(int2 *__restrict__ col, int *__restrict__ nonzero, const int4 *__restrict__ info,
+                                   const int2 *__restrict__ fn, const int *__restrict__ pairs,
+                                   const long long *__restrict__ mol, int nmol, long long nrows) {
+    const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (r > nrows) return;
+    if (r == nrows) {
+        nonzero[r] = 0;
+        return;
+    }
+    const int m = gather_mol_of(mol, nmol, r);
     const long long ij = r - __ldg(&mol[4 * m + 3]);
     const long long fb = __ldg(&mol[4 * m]), pb = __ldg(&mol[4 * m + 1]);
     const long long i = untri_f(ij), j = ij - i * (i + 1) / 2;
@@ -435,63 +446,100 @@ __global__ void gather_cols_kernel(int2 *__restrict__ col, double *__restrict__ 
     const int P = __ldg(&pairs[pb + (long long)fi.x * (fi.x + 1) / 2 + fj.x]);
     const int ca = (P & 1) ? fj.y : fi.y, cb = (P & 1) ? fi.y : fj.y;
     const bool zero = __ldg(&info[P >> 5]).y == 0;
-    col[__ldg(&mol[4 * m + 3]) + ij] = make_int2(zero ? -1 : ((P >> 5) << 4) | ((P >> 1) & 15), (ca << 16) | cb);
-    if (colq) colq[__ldg(&mol[4 * m + 3]) + ij] = __ldg(&bnd[P >> 5]).x;
+    col[r] = make_int2(zero ? -1 : ((P >> 5) << 4) | ((P >> 1) & 15), (ca << 16) | cb);
+    nonzero[r] = !zero;
+}
+
+// The columns that are not zero, molecule by molecule in ascending kl: list[pos[r]] = {kl, x, y, 0}
+// with colq the Qabs of the column's pair (plans that screen quartets), index[(mol[4m+3] >> 10) + m +
+// (kl >> 10)] = list position of the first column at or after kl for kl a multiple of 1024, and
+// end[m] the molecule's end in the list.
+constexpr int kGatherIndexShift = 10;
+__global__ void gather_list_kernel(const int2 *__restrict__ col, const int *__restrict__ pos,
+                                   const double2 *__restrict__ bnd, const long long *__restrict__ mol, int nmol,
+                                   long long nrows, int4 *__restrict__ list, double *__restrict__ colq,
+                                   int *__restrict__ index, int *__restrict__ end) {
+    const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= nrows) return;
+    const int m = gather_mol_of(mol, nmol, r);
+    const long long cbase = __ldg(&mol[4 * m + 3]), kl = r - cbase;
+    const int2 c = col[r];
+    const int p = pos[r];
+    if (c.x >= 0) {
+        list[p] = make_int4((int)kl, c.x, c.y, 0);
+        if (colq) colq[p] = __ldg(&bnd[c.x >> 4]).x;
+    }
+    if ((kl & ((1 << kGatherIndexShift) - 1)) == 0) index[(cbase >> kGatherIndexShift) + m + (kl >> kGatherIndexShift)] = p;
+    if (r + 1 == nrows || (m + 1 < nmol && r + 1 == __ldg(&mol[4 * (m + 1) + 3]))) end[m] = pos[r + 1];
 }
 
 // Second phase of the two-phase output: the packed vector written from the scratch blocks, one
 // shell pair P at a time.  A block of threads takes the next pair from units[] (heaviest first,
-// through an atomic counter) and writes all of P's rows (function pairs ij of P) column by
-// column: each thread takes a column kl, reads its descriptor once, and stores that column of
-// every row of P with kl <= ij.  The stores of one row are coalesced; the scratch entries of a
-// quartet (P, Q) for all of P's rows lie in one block, read by the same threads in the
-// same pass, so each scratch sector is fetched once.  Each entry comes from the block and
-// component the direct path would have stored it from: the quartet's bra is the pair of the
-// higher class, or of the later list position within a class (P for the diagonal quartet
-// P == Q); a pair's components are taken in its A, B orientation, with the larger component
-// first within a same-shell pair, as the direct store conditions pick.  With quartet
-// screening, the entries of a screened quartet are written as 0 without reading the scratch:
-// plans that screen end each bra's ket run after its last unscreened ket, so no chunk computes
-// the rest.
+// through an atomic counter) and writes all of P's rows (function pairs ij of P), a stretch of
+// columns at a time: first the rows' stretches are cleared with 16-byte stores (not where every
+// column of the stretch is computed), then each thread takes columns kl of the list of nonzero
+// columns, reads a column's descriptor once, and stores that column of every row of P with kl <= ij
+// over the zeros.  A stretch is short enough (64 KB of rows for small pairs) that its zeros are still
+// in L2 when the entries land on them, so DRAM sees each line once.  The scratch entries of a quartet
+// (P, Q) for all of P's rows lie in one block, read by the same threads in the same pass, so each
+// scratch sector is fetched once.  Each entry comes from the block and component the direct path
+// would have stored it from: the quartet's bra is the pair of the higher class, or of the later
+// list position within a class (P for the diagonal quartet P == Q); a pair's components are taken in
+// its A, B orientation, with the larger component first within a same-shell pair, as the direct
+// store conditions pick.  Zeros without a scratch read: pairs without kept primitive pairs (P's
+// rows, or columns not in the list) and, with quartet screening, columns whose quartet is screened
+// (plans that screen end each bra's ket run after its last unscreened ket, so no chunk computes the
+// rest).  Most entries are such zeros (78 % of a batch's integrals, 93 % with screening at 5e-10),
+// more than half of them in rows that are all zeros (zero_rows_kernel).  Measured on B200 over 1.17e9
+// integrals, FP64 / screened: 1.82 / 1.16 ms for the rows with entries, against 2.03 / 1.58 ms for
+// a form that visited every column; stretches of 4 times the length 2.48 / 1.44 (their zeros leave
+// L2 first), of a quarter 2.16 / 1.6, two columns a pass for the larger pairs 1.85 / 1.17, 40
+// registers and six blocks per SM 2.1 / 1.4.  Bound by the latency of its scratch loads: each is an
+// 8-byte entry of another quartet's block.
 constexpr int kGatherMaxRows = 100;  // components of an (ff) pair
 
-// The columns of one shell pair P for the gather: NC columns per thread and pass (kl,
-// kl + kGatherThreads, ...), their descriptor loads first, then the scratch loads of NR rows of
-// each column (NC * NR in flight), then their stores.  RMAX > 0: P has at most RMAX rows, known
-// at compile time (RMAX <= NR: one row step per pass, no loop).  (Measured on B200: NC = 2,
-// NR = 4 with the small pairs' copies specialised beats more columns or rows per pass and
-// prefetching the next pass's descriptors, which cost occupancy.)
+// n zeros at p, by the block.
+__device__ __forceinline__ void zero_run(double *__restrict__ p, long long n) {
+    if (n <= 0) return;
+    const int head = (int)((reinterpret_cast<size_t>(p) >> 3) & 1);  // rows start at any 8-byte address
+    if (threadIdx.x == 0 && head) p[0] = 0.0;
+    double2 *__restrict__ v = reinterpret_cast<double2 *>(p + head);
+    const long long nv = (n - head) >> 1;
+    for (long long k = threadIdx.x; k < nv; k += kGatherThreads) v[k] = make_double2(0.0, 0.0);
+    if (threadIdx.x == 0 && ((n - head) & 1)) p[n - 1] = 0.0;
+}
+
+// The listed columns [j0, j1) of one shell pair P for the gather: NC columns per thread and pass,
+// their descriptor loads first, then the scratch loads of NR rows of each column (NC * NR in
+// flight), then their stores.  RMAX > 0: P has at most RMAX rows, known at compile time (RMAX <= NR:
+// one row step per pass, no loop).
 template <int NC, int NR, int RMAX>
 __device__ __forceinline__ void gather_pair_columns(
-    double *__restrict__ obase, const double *__restrict__ scratch, const int2 *__restrict__ col,
-    const double *__restrict__ colq, long long cbase, const long long (*reg)[kNumPairClasses][5],
+    double *__restrict__ obase, const double *__restrict__ scratch, const int4 *__restrict__ list,
+    const double *__restrict__ colq, int j0, int j1, const long long (*reg)[kNumPairClasses][5],
     const long long *s_ij, const long long *s_tri, const int *s_rc, int R, int posP, int clsP,
     double qP, double screen_cut) {
     if (RMAX == 1) R = 1;
     const long long ijmax = s_ij[R - 1];  // rows are in increasing ij
     const int nP = c_pair_na[clsP] * c_pair_nb[clsP];
-    for (long long kl0 = threadIdx.x; kl0 <= ijmax; kl0 += NC * kGatherThreads) {
+    for (int jj = j0 + threadIdx.x; jj < j1; jj += NC * kGatherThreads) {
         const double *src[NC];
-        long long kl[NC];
-        int r0[NC], rs[NC];
-        bool zero[NC];
+        int kl[NC], r0[NC], rs[NC];
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-            kl[c] = kl0 + c * kGatherThreads;
-            const bool on = kl[c] <= ijmax;
-            const int2 qe = on ? __ldg(&col[cbase + kl[c]]) : make_int2(clsP, 0);
-            // a quartet of a pair without kept primitive pairs is 0, and so is a screened one (the
-            // class kernels' test, Qabs_P Qabs_Q < screen_cut); its block is not read (no chunk
-            // may have computed it)
-            const bool scr = on && screen_cut > 0.0 && qP * __ldg(&colq[cbase + kl[c]]) < screen_cut;
-            zero[c] = scr | (qe.x < 0);
+            const int j = jj + c * kGatherThreads;
+            const int4 qe = j < j1 ? __ldg(&list[j]) : make_int4(INT_MAX, 0, 0, 0);
+            // a screened quartet (the class kernels' test, Qabs_P Qabs_Q < screen_cut) stays 0; its
+            // block is not read (no chunk may have computed it)
+            const bool on = qe.x <= ijmax && !(screen_cut > 0.0 && j < j1 && qP * __ldg(&colq[j]) < screen_cut);
+            kl[c] = qe.x;
             src[c] = scratch;
             rs[c] = 0;
-            if (!zero[c]) {
-                // the column's scratch block and component (skipped for screened columns, most
-                // of a screened plan's)
-                const int posQ = on ? qe.x >> 4 : posP, clsQ = qe.x & 15;
-                const int qa = qe.y >> 16, qb = qe.y & 0xffff;
+            r0[c] = R;
+            if (on) {
+                // the column's scratch block and component
+                const int posQ = qe.y >> 4, clsQ = qe.y & 15;
+                const int qa = qe.z >> 16, qb = qe.z & 0xffff;
                 const bool braP = clsP > clsQ || (clsP == clsQ && posP >= posQ);
                 const long long *rg = reg[braP ? 0 : 1][clsQ];
                 const int bpos = braP ? posP : posQ, kpos = braP ? posQ : posP;
@@ -501,11 +549,11 @@ __device__ __forceinline__ void gather_pair_columns(
                 const int nq = c_pair_na[clsQ] * c_pair_nb[clsQ], qc = qa * c_pair_nb[clsQ] + qb;
                 rs[c] = braP ? nq : 1;
                 src[c] = scratch + rg[0] + slot * rg[4] + (braP ? qc : qc * nP);
+                // rows with ij >= kl: a suffix of the increasing row list
+                int r = 0;
+                while (r < R && s_ij[r] < kl[c]) ++r;
+                r0[c] = r;
             }
-            // rows with ij >= kl: a suffix of the increasing row list (none past ijmax)
-            int r = 0;
-            while (r < R && s_ij[r] < kl[c]) ++r;
-            r0[c] = on ? r : R;
         }
         int rmin = r0[0];
 #pragma unroll
@@ -516,7 +564,7 @@ __device__ __forceinline__ void gather_pair_columns(
             for (int c = 0; c < NC; ++c)
 #pragma unroll
                 for (int t = 0; t < NR; ++t)
-                    v[c][t] = (r + t < R && r + t >= r0[c] && !zero[c]) ? __ldg(src[c] + s_rc[r + t] * rs[c]) : 0.0;
+                    v[c][t] = (r + t < R && r + t >= r0[c]) ? __ldg(src[c] + s_rc[r + t] * rs[c]) : 0.0;
 #pragma unroll
             for (int c = 0; c < NC; ++c)
 #pragma unroll
@@ -527,36 +575,104 @@ __device__ __forceinline__ void gather_pair_columns(
     }
 }
 
-__global__ void __launch_bounds__(kGatherThreads) gather_packed_kernel(
-    double *__restrict__ out, const double *__restrict__ scratch, const int2 *__restrict__ col,
-    const double *__restrict__ colq, const long long *__restrict__ region, const long long *__restrict__ mol,
-    const int4 *__restrict__ units, long long nunits, int *__restrict__ counter, int nmol,
-    const double2 *__restrict__ bnd, const double *__restrict__ qmax, double screen_cut) {
+// The units (shell pairs) whose rows are all zeros -- pairs without kept primitive pairs, and with
+// quartet screening pairs whose every quartet is screened (Qabs_P times the molecule's largest Qabs
+// below the cutoff) -- go to the end of the list, the others keep their order at its front:
+// flag[u] = 1 for those (flag[n] = 0), pos their prefix sums.
+__global__ void unit_flag_kernel(const int4 *__restrict__ units, long long n, const int2 *__restrict__ col,
+                                 const long long *__restrict__ mol, const double2 *__restrict__ bnd,
+                                 const double *__restrict__ qmax, double screen_cut, int *__restrict__ flag) {
+    const long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (u > n) return;
+    int f = 0;
+    if (u < n) {
+        const int4 un = units[u];
+        const int2 pe = col[mol[4 * un.x + 3] + (long long)un.y * (un.y + 1) / 2 + un.z];
+        f = pe.x >= 0 && !(screen_cut > 0.0 && bnd[pe.x >> 4].x * qmax[un.x] < screen_cut);
+    }
+    flag[u] = f;
+}
+
+__global__ void unit_place_kernel(const int4 *__restrict__ units, long long n, const int *__restrict__ pos,
+                                  int4 *__restrict__ placed, int *__restrict__ n_live) {
+    const long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (u >= n) return;
+    const int p = pos[u];
+    placed[pos[u + 1] > p ? p : n - 1 - (u - p)] = units[u];
+    if (u == 0) *n_live = pos[n];
+}
+
+struct GatherArgs {
+    double *out;
+    const double *scratch;
+    const int2 *col;              // gather_cols_kernel
+    const int4 *list;             // gather_list_kernel
+    const double *colq;
+    const int *index, *end;
+    const long long *region, *mol;
+    long long nrows;
+    const int4 *units;            // unit_place_kernel
+    const int *n_live;            // units with entries; the others, from there on, are zeros
+    long long nunits;
+    int *counter;                 // the gather's next unit; counter[1]: the zero rows'
+
+    int nmol;
+    const double2 *bnd;
+    double screen_cut;
+};
+
+// The rows of the units that are all zeros: contiguous runs, at DRAM's write rate (5.1 GB in 0.83 ms).
+// Nothing else writes them, so this kernel runs beside the class kernels, which leave DRAM idle, with
+// two blocks per SM (execute of 1.17e9 integrals, FP64 / screened, with 1, 1.5, 2, 3 and 4 blocks
+// per SM: 6.87 / 5.16, 6.79 / 4.92, 6.84 / 4.88, 6.96 / 5.07, 7.07 / 5.20 ms).
+__global__ void __launch_bounds__(kGatherThreads) zero_rows_kernel(const GatherArgs A) {
+    __shared__ int s_unit;
+    const long long first = __ldg(A.n_live);
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) s_unit = atomicAdd(A.counter + 1, 1);
+        __syncthreads();
+        // the list's end holds the heavy units
+        const long long u = A.nunits - 1 - s_unit;
+        if (u < first) return;
+        const int4 un = __ldg(&A.units[u]);
+        const int nI = un.w & 255, nJ = (un.w >> 8) & 255, same = (un.w >> 16) & 1;
+        double *__restrict__ obase = A.out + __ldg(&A.mol[4 * un.x + 2]);
+        for (int a = 0; a < nI; ++a) {
+            const long long i = un.y + a;
+            for (int b = 0; b < (same ? a + 1 : nJ); ++b) {
+                const long long ij = i * (i + 1) / 2 + un.z + b;
+                zero_run(obase + ij * (ij + 1) / 2, ij + 1);
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kGatherThreads) gather_packed_kernel(const GatherArgs A) {
     // [P as bra, P as ket][class of the other pair]: {scratch offset, first bra, first ket,
     // kets, block size}
     __shared__ long long reg[2][kNumPairClasses][5];
     __shared__ long long s_ij[kGatherMaxRows], s_tri[kGatherMaxRows];
     __shared__ int s_rc[kGatherMaxRows];
     __shared__ long long s_unit;
+    const double screen_cut = A.screen_cut;
     for (;;) {
         __syncthreads();  // the previous unit's readers are done with the shared tables
-        if (threadIdx.x == 0) s_unit = atomicAdd(counter, 1);
+        if (threadIdx.x == 0) s_unit = atomicAdd(A.counter, 1);
         __syncthreads();
         const long long u = s_unit;
-        if (u >= nunits) return;
-        const int4 un = __ldg(&units[u]);
+        if (u >= __ldg(A.n_live)) return;
+        const int4 un = __ldg(&A.units[u]);
         const int m = un.x, fi0 = un.y, fj0 = un.z;
         const int nI = un.w & 255, nJ = (un.w >> 8) & 255, same = (un.w >> 16) & 1;
-        const long long cbase = __ldg(&mol[4 * m + 3]);
-        double *__restrict__ obase = out + __ldg(&mol[4 * m + 2]);
+        const long long cbase = __ldg(&A.mol[4 * m + 3]);
+        double *__restrict__ obase = A.out + __ldg(&A.mol[4 * m + 2]);
         // P's rows: ij, the row's first packed index tri(ij), and the row's component index in
         // P's A, B orientation
-        const int2 pe = __ldg(&col[cbase + (long long)fi0 * (fi0 + 1) / 2 + fj0]);
-        // a pair without kept primitive pairs: its rows are zeros (written below; class 0 stands in)
-        const bool zeroP = pe.x < 0;
-        const int posP = zeroP ? 0 : pe.x >> 4, clsP = zeroP ? 0 : pe.x & 15;
+        const int2 pe = __ldg(&A.col[cbase + (long long)fi0 * (fi0 + 1) / 2 + fj0]);
+        const int posP = pe.x >> 4, clsP = pe.x & 15;
         const int nbP = c_pair_nb[clsP];
-        const double qP = screen_cut > 0.0 ? __ldg(&bnd[posP]).x : 0.0;
+        const double qP = screen_cut > 0.0 ? __ldg(&A.bnd[posP]).x : 0.0;
         int R = 0;
         for (int a = 0; a < nI; ++a) R += same ? a + 1 : nJ;
         for (int r = threadIdx.x; r < R; r += kGatherThreads) {
@@ -564,7 +680,7 @@ __global__ void __launch_bounds__(kGatherThreads) gather_packed_kernel(
             if (same) { while (b > a) { b -= a + 1; ++a; } }
             else { a = r / nJ; b = r - a * nJ; }
             const long long i = fi0 + a, j = fj0 + b, ij = i * (i + 1) / 2 + j;
-            const int2 re = __ldg(&col[cbase + ij]);
+            const int2 re = __ldg(&A.col[cbase + ij]);
             s_ij[r] = ij;
             s_tri[r] = ij * (ij + 1) / 2;
             s_rc[r] = (re.y >> 16) * nbP + (re.y & 0xffff);
@@ -573,32 +689,35 @@ __global__ void __launch_bounds__(kGatherThreads) gather_packed_kernel(
             const int o = threadIdx.x / kNumPairClasses, t = threadIdx.x % kNumPairClasses;
             const int x = o == 0 ? clsP : t, y = o == 0 ? t : clsP;
             if (x >= y) {
-                const long long *rg = region + kRegionFields * (((long long)x * kNumPairClasses + y) * nmol + m);
+                const long long *rg = A.region + kRegionFields * (((long long)x * kNumPairClasses + y) * A.nmol + m);
                 for (int f = 0; f < kRegionFields; ++f) reg[o][t][f] = __ldg(&rg[f]);
                 reg[o][t][4] = (long long)c_pair_na[x] * c_pair_nb[x] * c_pair_na[y] * c_pair_nb[y];
             }
         }
         __syncthreads();
-        if (zeroP || (screen_cut > 0.0 && qP * __ldg(&qmax[m]) < screen_cut)) {
-            // P has no kept primitive pairs, or every quartet of P is screened (Qabs_P times the
-            // molecule's largest Qabs is below the cutoff): its rows are zeros, written as
-            // contiguous runs with no descriptor or scratch loads
-            for (int r = 0; r < R; ++r) {
-                const long long t0 = s_tri[r], n = s_ij[r] + 1;
-                for (long long k = threadIdx.x; k < n; k += kGatherThreads) obase[t0 + k] = 0.0;
+        const long long ijmax = s_ij[R - 1];
+        const long long nrowsM = (m + 1 < A.nmol ? __ldg(&A.mol[4 * m + 7]) : A.nrows) - cbase;
+        const int *__restrict__ index = A.index + (cbase >> kGatherIndexShift) + m;
+        const long long width = max(1 << kGatherIndexShift, (kGatherStretch / R) & ~((1 << kGatherIndexShift) - 1));
+        for (long long c0 = 0; c0 <= ijmax; c0 += width) {
+            const long long c1 = c0 + width;
+            const int j0 = __ldg(&index[c0 >> kGatherIndexShift]);
+            const int j1 = c1 < nrowsM ? __ldg(&index[c1 >> kGatherIndexShift]) : __ldg(&A.end[m]);
+            if (screen_cut > 0.0 || j1 - j0 < min(c1, nrowsM) - c0) {
+                for (int r = 0; r < R; ++r) zero_run(obase + s_tri[r] + c0, min(c1, s_ij[r] + 1) - c0);
+                __syncthreads();  // the zeros come before the entries
             }
-            continue;
+            // pairs of one or a few rows (ss, sp) are most of the units: their copies have no row loop
+            if (R == 1)
+                gather_pair_columns<4, 1, 1>(obase, A.scratch, A.list, A.colq, j0, j1, reg, s_ij, s_tri, s_rc, R, posP,
+                                             clsP, qP, screen_cut);
+            else if (R <= 4)
+                gather_pair_columns<1, 4, 4>(obase, A.scratch, A.list, A.colq, j0, j1, reg, s_ij, s_tri, s_rc, R, posP,
+                                             clsP, qP, screen_cut);
+            else
+                gather_pair_columns<1, 4, 0>(obase, A.scratch, A.list, A.colq, j0, j1, reg, s_ij, s_tri, s_rc, R, posP,
+                                             clsP, qP, screen_cut);
         }
-        // pairs of one or a few rows (ss, sp) are most of the units: their copies have no row loop
-        if (R == 1)
-            gather_pair_columns<2, 1, 1>(obase, scratch, col, colq, cbase, reg, s_ij, s_tri, s_rc, R, posP, clsP,
-                                         qP, screen_cut);
-        else if (R <= 4)
-            gather_pair_columns<2, 4, 4>(obase, scratch, col, colq, cbase, reg, s_ij, s_tri, s_rc, R, posP, clsP,
-                                         qP, screen_cut);
-        else
-            gather_pair_columns<2, 4, 0>(obase, scratch, col, colq, cbase, reg, s_ij, s_tri, s_rc, R, posP, clsP,
-                                         qP, screen_cut);
     }
 }
 
@@ -974,8 +1093,8 @@ static void plan_release_device(molints_plan *p) {
     p->prof_ev.clear();
     void *bufs[] = {p->sh_xyz, p->expn, p->ncoef, p->sh_poff, p->pair_ab, p->info, p->pp_src, p->pbk,
                     p->geo, p->pp, p->bnd, p->chunks, p->counters, p->mol_out, p->qcon,
-                    p->chunk_slot, p->g_fn, p->g_pair, p->g_region, p->g_mol, p->g_col, p->g_colq,
-                    p->g_qmax, p->g_units, p->gq, p->gq_mol, p->sh_L, p->sh_K, p->sh_fn};
+                    p->chunk_slot, p->g_fn, p->g_pair, p->g_region, p->g_mol, p->g_col, p->g_list, p->g_colq, p->g_index, p->g_end, p->g_nlive,
+                    p->g_units, p->gq, p->gq_mol, p->sh_L, p->sh_K, p->sh_fn};
     for (void *b : bufs) dev_free(p->ctx, b);
     p->ctx->held -= p->bytes;
     p->ctx = nullptr;
@@ -1395,7 +1514,10 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     // bra-major (the triangle q <= p for equal classes); region_h[((x nc + y) nmol + m) 4 ..] =
     // {offset in doubles, first bra pair, first ket pair, ket pairs}.  Quartet slot t's block
     // starts at offset + t * block.
-    if (npair >= (1 << 26)) p->two_phase = 0;  // the gather's pair entries hold the position in 26 bits
+    // the gather's pair entries hold the position in 26 bits, its column list counts in 31
+    int64_t fn_pairs = 0;
+    for (int m = 0; m < nmol; ++m) fn_pairs += mol_nbf[m] * (mol_nbf[m] + 1) / 2;
+    if (npair >= (1 << 26) || fn_pairs >= INT32_MAX) p->two_phase = 0;
     auto ncomp_of = [](int x, int y) {
         return (int64_t)ncart(kPairClassLa[x]) * ncart(kPairClassLb[x]) * ncart(kPairClassLa[y]) * ncart(kPairClassLb[y]);
     };
@@ -1468,7 +1590,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     const size_t t_off = tv.take<long long>((size_t)n_items + 1);
     const size_t t_sum = tv.take<long long>(kNumClassPairs + 2), t_ccost = tv.take<double>(kNumClassPairs);
     const size_t cub_bytes = std::max(plan_build_temp_bytes(npair), queue_count_temp_bytes(n_items));
-    const size_t t_cub = tv.take<char>(cub_bytes);
+    const size_t t_cub = tv.take<char>(cub_bytes), t_units = tv.take<int4>(tp ? npe_all : 0);
     Carve sv;
     // read back: class-pair chunk offsets and the count of pairs without kept primitive pairs,
     // class-pair costs, kept primitive pairs, bad-shell flag
@@ -1587,7 +1709,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     rc = rc ? rc : dev_alloc(ctx, &p->pp_src, (size_t)nall, &p->bytes);
     rc = rc ? rc : dev_alloc(ctx, &p->pbk, (size_t)nall, &p->bytes);
     rc = rc ? rc : dev_alloc(ctx, &p->pp, (size_t)nall, &p->bytes);
-    rc = rc ? rc : dev_alloc(ctx, &p->counters, (size_t)nc2 + 1, &p->bytes);  // + the gather's or the g kernel's
+    rc = rc ? rc : dev_alloc(ctx, &p->counters, (size_t)nc2 + 2, &p->bytes);  // + the gather's two or the g kernel's
     rc = rc ? rc : dev_alloc(ctx, &p->mol_out, (size_t)std::max(nmol, 1), &p->bytes);
     if (tp) {
         rc = rc ? rc : dev_alloc(ctx, &p->g_fn, (size_t)std::max<int64_t>(nfn_all, 1), &p->bytes);
@@ -1595,9 +1717,12 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
         rc = rc ? rc : dev_alloc(ctx, &p->g_region, region_h.size(), &p->bytes);
         rc = rc ? rc : dev_alloc(ctx, &p->g_mol, (size_t)nmol * 4, &p->bytes);
         rc = rc ? rc : dev_alloc(ctx, &p->g_col, (size_t)std::max<int64_t>(nrows_all, 1), &p->bytes);
+        rc = rc ? rc : dev_alloc(ctx, &p->g_list, (size_t)std::max<int64_t>(nrows_all, 1), &p->bytes);
+        rc = rc ? rc : dev_alloc(ctx, &p->g_index, (size_t)(nrows_all >> kGatherIndexShift) + nmol + 1, &p->bytes);
+        rc = rc ? rc : dev_alloc(ctx, &p->g_nlive, 1, &p->bytes);
+        rc = rc ? rc : dev_alloc(ctx, &p->g_end, (size_t)std::max(nmol, 1), &p->bytes);
         if (opts.screen_cutoff > 0.0) {
             rc = rc ? rc : dev_alloc(ctx, &p->g_colq, (size_t)std::max<int64_t>(nrows_all, 1), &p->bytes);
-            rc = rc ? rc : dev_alloc(ctx, &p->g_qmax, (size_t)std::max(nmol, 1), &p->bytes);
         }
         rc = rc ? rc : dev_alloc(ctx, &p->g_units, (size_t)std::max<int64_t>(npe_all, 1), &p->bytes);
     }
@@ -1626,7 +1751,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
         (tp && ((e = h2d(p->g_region, o_greg, region_h.size() * sizeof(long long))) ||
                 (e = h2d(p->g_fn, o_gfn, (size_t)nfn_all * sizeof(int2))) ||
                 (e = h2d(p->g_mol, o_gmol, (size_t)nmol * 4 * sizeof(long long))) ||
-                (e = h2d(p->g_units, o_gunits, (size_t)npe_all * sizeof(int4))))) ||
+                (e = h2d(tmp + t_units, o_gunits, (size_t)npe_all * sizeof(int4))))) ||
         (e = cudaMemsetAsync(p->counters + nc2, 0, sizeof(int), s)) ||
         (e = cudaMemsetAsync(tmp + t_qmax, 0, (size_t)std::max(nmol, 1) * sizeof(unsigned long long), s)) ||
         (e = cudaMemsetAsync(tmp + t_sum, 0, (kNumClassPairs + 2) * sizeof(long long), s)) ||
@@ -1770,13 +1895,38 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
         if (e != cudaSuccess) { release_temp(); plan_free(p); return cuda_fail(ctx, e, "plan_create work queues"); }
     }
     if (tp && nrows_all > 0) {
-        gather_cols_kernel<<<(unsigned)((nrows_all + 255) / 256), 256, 0, s>>>(p->g_col, p->g_colq, p->bnd,
-                                                                            p->info, p->g_fn, p->g_pair,
-                                                                            p->g_mol, nmol, nrows_all);
+        // the gather's columns and the list of the nonzero ones (their positions by a prefix sum)
+        Carve gv;
+        const int64_t nscan = std::max(nrows_all, p->n_units) + 1;
+        const size_t g_flag = gv.take<int>(nscan), g_pos = gv.take<int>(nscan);
+        const size_t scan_bytes = gather_scan_temp_bytes(nscan), g_scan = gv.take<char>(scan_bytes);
+        char *gtmp = nullptr;
+        rc = dev_alloc(ctx, &gtmp, gv.at, &temp_tally);
+        if (rc) { release_temp(); plan_free(p); return rc; }
+        int *flag = reinterpret_cast<int *>(gtmp + g_flag), *pos = reinterpret_cast<int *>(gtmp + g_pos);
+        gather_cols_kernel<<<(unsigned)((nrows_all + 256) / 256), 256, 0, s>>>(p->g_col, flag, p->info, p->g_fn,
+                                                                               p->g_pair, p->g_mol, nmol, nrows_all);
         e = cudaGetLastError();
-        if (!e && p->g_qmax)  // the molecules' Qabs bounds (doubles as bits) outlive the build
-            e = cudaMemcpyAsync(p->g_qmax, tmp + t_qmax, (size_t)nmol * sizeof(double), cudaMemcpyDeviceToDevice, s);
+        if (!e) e = gather_scan(flag, pos, nrows_all + 1, gtmp + g_scan, scan_bytes, s);
+        if (!e) {
+            gather_list_kernel<<<(unsigned)((nrows_all + 255) / 256), 256, 0, s>>>(
+                p->g_col, pos, p->bnd, p->g_mol, nmol, nrows_all, p->g_list, p->g_colq, p->g_index, p->g_end);
+            e = cudaGetLastError();
+        }
+        if (!e) {
+            // (the molecules' Qabs bounds are doubles as bits)
+            const int4 *u0 = reinterpret_cast<const int4 *>(tmp + t_units);
+            unit_flag_kernel<<<(unsigned)((p->n_units + 256) / 256), 256, 0, s>>>(
+                u0, p->n_units, p->g_col, p->g_mol, p->bnd, reinterpret_cast<const double *>(tmp + t_qmax),
+                opts.screen_cutoff, flag);
+            e = gather_scan(flag, pos, p->n_units + 1, gtmp + g_scan, scan_bytes, s);
+            unit_place_kernel<<<(unsigned)((p->n_units + 255) / 256), 256, 0, s>>>(u0, p->n_units, pos, p->g_units,
+                                                                                  p->g_nlive);
+            if (!e) e = cudaGetLastError();
+        }
+        dev_free(ctx, gtmp);
         if (e) { release_temp(); plan_free(p); return cuda_fail(ctx, e, "plan_create gather columns"); }
+        p->n_rows = nrows_all;
     }
     release_temp();
     p->plan_ms[2] = ms_since(t_phase);
@@ -1835,7 +1985,7 @@ static int plan_enqueue(molints_plan *p, double *out_device, bool timing, JKOut 
         return err == cudaSuccess ? 0 : cuda_fail(ctx, err, "cudaEventRecord");
     };
     if (timing) MI_CUDA(ctx, cudaEventRecord(ctx->ev0, s));
-    MI_CUDA(ctx, cudaMemsetAsync(p->counters, 0, sizeof(int) * (kNumPairClasses * kNumPairClasses + 1), s));
+    MI_CUDA(ctx, cudaMemsetAsync(p->counters, 0, sizeof(int) * (kNumPairClasses * kNumPairClasses + 2), s));
     // Direct plans: the quartets no chunk holds (those of pairs without kept primitive pairs, and
     // with quartet screening those past each bra's last unscreened ket) get their zeros from
     // clearing the whole output first, a streaming write instead of scattered 8-byte stores: up to
@@ -1881,6 +2031,20 @@ static int plan_enqueue(molints_plan *p, double *out_device, bool timing, JKOut 
     int fp32_launches = 0;
     if (nside > 0) MI_CUDA(ctx, cudaEventRecord(ctx->fork, s));
     for (int i = 0; i < nside; ++i) MI_CUDA(ctx, cudaStreamWaitEvent(ctx->side[i], ctx->fork, 0));
+    const bool gather = p->two_phase && !jk.J && p->npacked > 0;
+    const GatherArgs G{out_device, ctx->scratch, p->g_col, p->g_list, p->g_colq, p->g_index, p->g_end, p->g_region,
+                       p->g_mol, p->n_rows, p->g_units, p->g_nlive, p->n_units,
+                       p->counters + kNumPairClasses * kNumPairClasses, p->nmol, p->bnd, p->opts.screen_cutoff};
+    cudaStream_t zs = nside ? ctx->side[molints_ctx::kSideTwoPhase] : s;
+    if (gather) {
+        // the all-zero rows, on a stream of their own until the end of the execute
+        if (nside) MI_CUDA(ctx, cudaStreamWaitEvent(zs, ctx->fork, 0));
+        if (int rc = mark(launches, "zero_rows", 0, zs)) return rc;
+        zero_rows_kernel<<<(int)std::min<int64_t>(2 * ctx->num_sms, p->n_units), kGatherThreads, 0, zs>>>(G);
+        if (int rc = mark(launches, "zero_rows", 1, zs)) return rc;
+        ++launches;
+        if (nside) MI_CUDA(ctx, cudaEventRecord(ctx->join[molints_ctx::kSideTwoPhase], zs));
+    }
     if (ngen) {
         // shell quartets with a g shell (never two-phase plans; no J/K digestion): entries of their
         // own, beside the class kernels on the first side stream
@@ -1932,7 +2096,7 @@ static int plan_enqueue(molints_plan *p, double *out_device, bool timing, JKOut 
         MI_CUDA(ctx, cudaEventRecord(ctx->join[i], ctx->side[i]));
         MI_CUDA(ctx, cudaStreamWaitEvent(s, ctx->join[i], 0));
     }
-    if (p->two_phase && !jk.J && p->npacked > 0) {
+    if (gather) {
         // second phase: the packed vector in order from the scratch blocks
         if (int rc = mark(launches, "gather_packed", 0, s)) return rc;
         // a persistent grid of gather_blocks blocks per SM; blocks beyond what the kernel's
@@ -1940,12 +2104,10 @@ static int plan_enqueue(molints_plan *p, double *out_device, bool timing, JKOut 
         // unit list done
         const int gb = p->gather_blocks > 0 ? p->gather_blocks : kGatherBlocksDefault;
         const int grid = (int)std::min<long long>((long long)ctx->num_sms * gb, p->n_units);
-        gather_packed_kernel<<<grid, kGatherThreads, 0, s>>>(out_device, ctx->scratch, p->g_col, p->g_colq, p->g_region,
-                                                             p->g_mol, p->g_units, p->n_units,
-                                                             p->counters + kNumPairClasses * kNumPairClasses,
-                                                             p->nmol, p->bnd, p->g_qmax, p->opts.screen_cutoff);
+        gather_packed_kernel<<<grid, kGatherThreads, 0, s>>>(G);
         if (int rc = mark(launches, "gather_packed", 1, s)) return rc;
         ++launches;
+        if (nside) MI_CUDA(ctx, cudaStreamWaitEvent(s, ctx->join[molints_ctx::kSideTwoPhase], 0));
     }
     MI_CUDA(ctx, cudaGetLastError());
     if (timing) MI_CUDA(ctx, cudaEventRecord(ctx->ev1, s));

@@ -316,4 +316,14 @@ cudaError_t queue_emit(const QueueSetup &S, const QueueArgs &A, const QueueEmitA
     return cudaGetLastError();
 }
 
+size_t gather_scan_temp_bytes(long long n) {
+    size_t a = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, a, (const int *)nullptr, (int *)nullptr, n);
+    return a;
+}
+
+cudaError_t gather_scan(const int *in, int *out, long long n, void *temp, size_t temp_bytes, cudaStream_t s) {
+    return cub::DeviceScan::ExclusiveSum(temp, temp_bytes, in, out, n, s);
+}
+
 }  // namespace molints

@@ -229,4 +229,8 @@ cudaError_t queue_emit(const QueueSetup &S, const QueueArgs &A, const QueueEmitA
                        size_t temp_bytes, cudaStream_t s);
 size_t queue_emit_temp_bytes(long long nq);
 
+// Exclusive prefix sums of n ints (the gather's list positions); temp: gather_scan_temp_bytes(n).
+cudaError_t gather_scan(const int *in, int *out, long long n, void *temp, size_t temp_bytes, cudaStream_t s);
+size_t gather_scan_temp_bytes(long long n);
+
 }  // namespace molints
