@@ -4,19 +4,19 @@
 namespace molints {
 void launch_eri_ssss(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_ssss(int mixed);
-void launch_schwarz_ssss(const PairTab &P, const BoysTab &B, int p0, int np, double2 *pbound, double *qout, int full, cudaStream_t s);
+void launch_schwarz_ssss(const PairTab &P, const BoysTab &B, int p0, int np, double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s);
 void launch_eri_psss(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_psss(int mixed);
 void launch_eri_psps(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_psps(int mixed);
-void launch_schwarz_psps(const PairTab &P, const BoysTab &B, int p0, int np, double2 *pbound, double *qout, int full, cudaStream_t s);
+void launch_schwarz_psps(const PairTab &P, const BoysTab &B, int p0, int np, double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s);
 void launch_eri_ppss(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_ppss(int mixed);
 void launch_eri_ppps(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_ppps(int mixed);
 void launch_eri_pppp(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_pppp(int mixed);
-void launch_schwarz_pppp(const PairTab &P, const BoysTab &B, int p0, int np, double2 *pbound, double *qout, int full, cudaStream_t s);
+void launch_schwarz_pppp(const PairTab &P, const BoysTab &B, int p0, int np, double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s);
 void launch_eri_dsss(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_dsss(int mixed);
 void launch_eri_dsps(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
@@ -25,7 +25,7 @@ void launch_eri_dspp(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_dspp(int mixed);
 void launch_eri_dsds(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_dsds(int mixed);
-void launch_schwarz_dsds(const PairTab &P, const BoysTab &B, int p0, int np, double2 *pbound, double *qout, int full, cudaStream_t s);
+void launch_schwarz_dsds(const PairTab &P, const BoysTab &B, int p0, int np, double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s);
 void launch_eri_dpss(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_dpss(int mixed);
 void launch_eri_dpps(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
@@ -36,7 +36,7 @@ void launch_eri_dpds(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_dpds(int mixed);
 void launch_eri_dpdp(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_dpdp(int mixed);
-void launch_schwarz_dpdp(const PairTab &P, const BoysTab &B, int p0, int np, double2 *pbound, double *qout, int full, cudaStream_t s);
+void launch_schwarz_dpdp(const PairTab &P, const BoysTab &B, int p0, int np, double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s);
 void launch_eri_fsss(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_fsss(int mixed);
 void launch_eri_fsps(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
@@ -49,7 +49,7 @@ void launch_eri_fsdp(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_fsdp(int mixed);
 void launch_eri_fsfs(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_fsfs(int mixed);
-void launch_schwarz_fsfs(const PairTab &P, const BoysTab &B, int p0, int np, double2 *pbound, double *qout, int full, cudaStream_t s);
+void launch_schwarz_fsfs(const PairTab &P, const BoysTab &B, int p0, int np, double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s);
 void launch_eri_ddss(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_ddss(int mixed);
 void launch_eri_ddps(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
@@ -62,7 +62,6 @@ void launch_eri_dddp(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_dddp(int mixed);
 void launch_eri_dddd(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_dddd(int mixed);
-void launch_schwarz_dddd(const PairTab &P, const BoysTab &B, int p0, int np, double2 *pbound, double *qout, int full, cudaStream_t s);
 void launch_eri_fpss(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
 int occupancy_eri_fpss(int mixed);
 void launch_eri_fpps(const EriQueue &Q, int mixed, int grid, cudaStream_t s);
@@ -89,7 +88,7 @@ void launch_rys_ppps(const EriQueue &Q, const RysTab &R, int mixed, int grid, cu
 int occupancy_rys_ppps(int mixed);
 void launch_rys_pppp(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_pppp(int mixed);
-void launch_rys_bound_pppp(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, double *qout, int full, cudaStream_t s);
+void launch_rys_bound_pppp(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s);
 void launch_rys_dsss(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_dsss(int mixed);
 void launch_rys_dsps(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
@@ -98,7 +97,7 @@ void launch_rys_dspp(const EriQueue &Q, const RysTab &R, int mixed, int grid, cu
 int occupancy_rys_dspp(int mixed);
 void launch_rys_dsds(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_dsds(int mixed);
-void launch_rys_bound_dsds(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, double *qout, int full, cudaStream_t s);
+void launch_rys_bound_dsds(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s);
 void launch_rys_dpss(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_dpss(int mixed);
 void launch_rys_dpps(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
@@ -109,7 +108,7 @@ void launch_rys_dpds(const EriQueue &Q, const RysTab &R, int mixed, int grid, cu
 int occupancy_rys_dpds(int mixed);
 void launch_rys_dpdp(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_dpdp(int mixed);
-void launch_rys_bound_dpdp(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, double *qout, int full, cudaStream_t s);
+void launch_rys_bound_dpdp(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s);
 void launch_rys_fsss(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_fsss(int mixed);
 void launch_rys_fsps(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
@@ -122,7 +121,7 @@ void launch_rys_fsdp(const EriQueue &Q, const RysTab &R, int mixed, int grid, cu
 int occupancy_rys_fsdp(int mixed);
 void launch_rys_fsfs(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_fsfs(int mixed);
-void launch_rys_bound_fsfs(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, double *qout, int full, cudaStream_t s);
+void launch_rys_bound_fsfs(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s);
 void launch_rys_ddss(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_ddss(int mixed);
 void launch_rys_ddps(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
@@ -137,7 +136,7 @@ void launch_rys_ddfs(const EriQueue &Q, const RysTab &R, int mixed, int grid, cu
 int occupancy_rys_ddfs(int mixed);
 void launch_rys_dddd(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_dddd(int mixed);
-void launch_rys_bound_dddd(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, double *qout, int full, cudaStream_t s);
+void launch_rys_bound_dddd(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s);
 void launch_rys_fpss(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_fpss(int mixed);
 void launch_rys_fpps(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
@@ -154,7 +153,7 @@ void launch_rys_fpdd(const EriQueue &Q, const RysTab &R, int mixed, int grid, cu
 int occupancy_rys_fpdd(int mixed);
 void launch_rys_fpfp(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_fpfp(int mixed);
-void launch_rys_bound_fpfp(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, double *qout, int full, cudaStream_t s);
+void launch_rys_bound_fpfp(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s);
 void launch_rys_dfss(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_dfss(int mixed);
 void launch_rys_dfps(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
@@ -173,7 +172,7 @@ void launch_rys_dffp(const EriQueue &Q, const RysTab &R, int mixed, int grid, cu
 int occupancy_rys_dffp(int mixed);
 void launch_rys_dfdf(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_dfdf(int mixed);
-void launch_rys_bound_dfdf(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, double *qout, int full, cudaStream_t s);
+void launch_rys_bound_dfdf(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s);
 void launch_rys_fdss(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_fdss(int mixed);
 void launch_rys_fdps(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
@@ -194,7 +193,7 @@ void launch_rys_fddf(const EriQueue &Q, const RysTab &R, int mixed, int grid, cu
 int occupancy_rys_fddf(int mixed);
 void launch_rys_fdfd(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_fdfd(int mixed);
-void launch_rys_bound_fdfd(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, double *qout, int full, cudaStream_t s);
+void launch_rys_bound_fdfd(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s);
 void launch_rys_ffss(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_ffss(int mixed);
 void launch_rys_ffps(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
@@ -217,13 +216,13 @@ void launch_rys_fffd(const EriQueue &Q, const RysTab &R, int mixed, int grid, cu
 int occupancy_rys_fffd(int mixed);
 void launch_rys_ffff(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_ffff(int mixed);
-void launch_rys_bound_ffff(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, double *qout, int full, cudaStream_t s);
+void launch_rys_bound_ffff(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s);
 typedef void (*EriLauncher)(const EriQueue &, int, int, cudaStream_t);
 typedef int (*EriOccupancy)(int);
-typedef void (*SchwarzLauncher)(const PairTab &, const BoysTab &, int, int, double2 *, double *, int, cudaStream_t);
+typedef void (*SchwarzLauncher)(const PairTab &, const BoysTab &, int, int, double2 *, const int *, unsigned long long *, double *, int, cudaStream_t);
 typedef void (*RysLauncher)(const EriQueue &, const RysTab &, int, int, cudaStream_t);
 typedef int (*RysOccupancy)(int);
-typedef void (*RysBoundLauncher)(const PairTab &, const RysTab &, int, int, double2 *, double *, int, cudaStream_t);
+typedef void (*RysBoundLauncher)(const PairTab &, const RysTab &, int, int, double2 *, const int *, unsigned long long *, double *, int, cudaStream_t);
 constexpr int kLmax = 3;      // shells up to f (Rys)
 constexpr int kLmaxHgp = 2;   // every class pair up to d has an HGP kernel
 constexpr int kNumPairClasses = 11;
@@ -371,7 +370,7 @@ static const char *const kSchwarzNames[11] = {
     "schwarz_ss", "schwarz_ps", "schwarz_pp", "schwarz_ds", "schwarz_dp", "schwarz_fs", "schwarz_dd", "schwarz_fp", "schwarz_df", "schwarz_fd", "schwarz_ff"
 };
 static const SchwarzLauncher kSchwarzLaunchers[11] = {
-    launch_schwarz_ssss, launch_schwarz_psps, launch_schwarz_pppp, launch_schwarz_dsds, launch_schwarz_dpdp, launch_schwarz_fsfs, launch_schwarz_dddd, nullptr, nullptr, nullptr, nullptr
+    launch_schwarz_ssss, launch_schwarz_psps, launch_schwarz_pppp, launch_schwarz_dsds, launch_schwarz_dpdp, launch_schwarz_fsfs, nullptr, nullptr, nullptr, nullptr, nullptr
 };
 static const RysBoundLauncher kRysBoundLaunchers[11] = {
     nullptr, nullptr, launch_rys_bound_pppp, launch_rys_bound_dsds, launch_rys_bound_dpdp, launch_rys_bound_fsfs, launch_rys_bound_dddd, launch_rys_bound_fpfp, launch_rys_bound_dfdf, launch_rys_bound_fdfd, launch_rys_bound_ffff

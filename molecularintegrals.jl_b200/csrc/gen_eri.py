@@ -51,6 +51,9 @@ MIXED_MIN_VRR = 40
 # chunk's blocks into dynamic shared memory (4 warps x 32 blocks x 8 B each: up to 162 KB) and
 # the warp copies them to the scratch as one contiguous run
 STAGE_MAX_OUT = 162
+# Pair classes whose bounds the Rys bound kernel computes although an HGP kernel exists: the HGP
+# (dd|dd) kernel's straight-line code takes 34 us for a handful of pairs
+RYS_BOUND = {(2, 2)}
 # J/K digestion: blocks of at most this many outputs are digested from registers; larger ones sit in
 # local memory, read by a loop over A's components
 JK_UNROLL_MAX_OUT = 36
@@ -344,7 +347,7 @@ def emit_class_pair(X, Y, rys=False):
                         for ic in range(nc) for id_ in range(nd))
     store_code = "\n".join(stores)
     schwarz = ""
-    if X == Y and not rys:
+    if X == Y and not rys and X not in RYS_BOUND:
         diag = []
         for ia in range(na):
             for ib in range(nb):
@@ -360,35 +363,48 @@ def emit_class_pair(X, Y, rys=False):
 //     pbound[k].y = w_k = sqrt(max over the VRR block |[e0|e0]_kk|), e = la..la+lb
 //   By the Schwarz inequality b_k b_l bounds |(a_k b_k|c_l d_l)| and w_k w_l bounds every
 //   entry of the VRR output block [e0|f0] that the HRR combines.
+//   qmax[mol[p]]: the largest sum of b_k (in list order) over the molecule's pairs, as bits.
 // full != 0: the contracted bound Q_p = sqrt(max |(ab|ab)|) into qout[p].
+// A warp per pair, its lanes over the primitive pairs (one thread per pair, over up to 49 primitive
+// pairs in turn, took 46 us for (ss) on B200).
 __global__ void __launch_bounds__(128) schwarz_kernel_{tag}(PairTab P, BoysTab B, int p0, int np,
-                                                          double2 *pbound, double *qout, int full) {{
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+                                                          double2 *pbound, const int *mol,
+                                                          unsigned long long *qmax, double *qout, int full) {{
+    const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (t >= np) return;
     const int p = p0 + t;
     const int4 in = __ldg(&P.info[p]);
     double res[{nout}];
     if (full) {{
+        if (lane) return;
         quartet_{tag}<double>(P, B, p, p, 0, in.y, 0, in.y, res);
         double m = 0.0;
 {diag}
         qout[p] = sqrt(m);
         return;
     }}
-    double acc[{nacc}];
-    for (int k = 0; k < in.y; ++k) {{
-        quartet_{tag}<double>(P, B, p, p, k, k + 1, k, k + 1, res, acc);
+    double acc[{nacc}], q = 0.0;
+    for (int k0 = 0; k0 < in.y; k0 += 32) {{
+        const int k = k0 + lane;
         double m = 0.0, w = 0.0;
+        if (k < in.y) {{
+            quartet_{tag}<double>(P, B, p, p, k, k + 1, k, k + 1, res, acc);
 {diag}
 {accdiag}
-        pbound[in.x + k] = make_double2(sqrt(m), sqrt(w));
+            m = sqrt(m);
+            pbound[in.x + k] = make_double2(m, sqrt(w));
+        }}
+        const int n = min(32, in.y - k0);
+        for (int x = 0; x < n; ++x) q += __shfl_sync(0xffffffffu, m, x);
     }}
+    // the sums are >= 0, so their bit patterns order like the values
+    if (lane == 0) atomicMax(&qmax[__ldg(&mol[p])], (unsigned long long)__double_as_longlong(q));
 }}
 
 void launch_schwarz_{tag}(const PairTab &P, const BoysTab &B, int p0, int np, double2 *pbound,
-                          double *qout, int full, cudaStream_t s) {{
+                          const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s) {{
     if (np <= 0) return;
-    schwarz_kernel_{tag}<<<(np + 127) / 128, 128, 0, s>>>(P, B, p0, np, pbound, qout, full);
+    schwarz_kernel_{tag}<<<(np + 3) / 4, 128, 0, s>>>(P, B, p0, np, pbound, mol, qmax, qout, full);
 }}
 """
     has32 = len(entries) >= MIXED_MIN_VRR and not rys
@@ -774,24 +790,26 @@ def emit_dispatch(pairs):
         t = tag_of(X, Y)
         lines.append(f"void launch_eri_{t}(const EriQueue &Q, int mixed, int grid, cudaStream_t s);")
         lines.append(f"int occupancy_eri_{t}(int mixed);")
-        if X == Y:
-            lines.append(f"void launch_schwarz_{t}(const PairTab &P, const BoysTab &B, int p0, "
-                         f"int np, double2 *pbound, double *qout, int full, cudaStream_t s);")
+        if X == Y and X not in RYS_BOUND:
+            lines.append(f"void launch_schwarz_{t}(const PairTab &P, const BoysTab &B, int p0, int np, "
+                         f"double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, "
+                         f"cudaStream_t s);")
     for X, Y in gen_rys.class_pairs():
         t = tag_of(X, Y)
         lines.append(f"void launch_rys_{t}(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);")
         lines.append(f"int occupancy_rys_{t}(int mixed);")
         if X == Y and not gen_rys.is_lane(X, Y):
             lines.append(f"void launch_rys_bound_{t}(const PairTab &P, const RysTab &R, int p0, int np, "
-                         f"double2 *pbound, double *qout, int full, cudaStream_t s);")
+                         f"double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, "
+                         f"cudaStream_t s);")
     lines.append("typedef void (*EriLauncher)(const EriQueue &, int, int, cudaStream_t);")
     lines.append("typedef int (*EriOccupancy)(int);")
-    lines.append("typedef void (*SchwarzLauncher)(const PairTab &, const BoysTab &, int, int, "
-                 "double2 *, double *, int, cudaStream_t);")
+    lines.append("typedef void (*SchwarzLauncher)(const PairTab &, const BoysTab &, int, int, double2 *, "
+                 "const int *, unsigned long long *, double *, int, cudaStream_t);")
     lines.append("typedef void (*RysLauncher)(const EriQueue &, const RysTab &, int, int, cudaStream_t);")
     lines.append("typedef int (*RysOccupancy)(int);")
-    lines.append("typedef void (*RysBoundLauncher)(const PairTab &, const RysTab &, int, int, "
-                 "double2 *, double *, int, cudaStream_t);")
+    lines.append("typedef void (*RysBoundLauncher)(const PairTab &, const RysTab &, int, int, double2 *, "
+                 "const int *, unsigned long long *, double *, int, cudaStream_t);")
     lines.append(f"constexpr int kLmax = {gen_rys.LMAX};      // shells up to f (Rys)")
     lines.append(f"constexpr int kLmaxHgp = {LMAX_ALL_HGP};   // every class pair up to d has an HGP kernel")
     lines.append(f"constexpr int kNumPairClasses = {len(cls)};")
@@ -854,7 +872,7 @@ def emit_dispatch(pairs):
     lines.append("    " + ", ".join(f'"schwarz_{tag_of(X, X)[:2]}"' for X in cls))
     lines.append("};")
     lines.append(f"static const SchwarzLauncher kSchwarzLaunchers[{n}] = {{")
-    lines.append("    " + ", ".join(f"launch_schwarz_{tag_of(X, X)}" if (X, X) in hgp else "nullptr"
+    lines.append("    " + ", ".join(f"launch_schwarz_{tag_of(X, X)}" if (X, X) in hgp and X not in RYS_BOUND else "nullptr"
                                    for X in cls))
     lines.append("};")
     lines.append(f"static const RysBoundLauncher kRysBoundLaunchers[{n}] = {{")

@@ -230,17 +230,19 @@ def emit_class_pair(X, Y):
     if diag:
         bound_kernel = f"""
 __global__ void __launch_bounds__(128) rys_bound_kernel_{tag}(PairTab P, RysTab R, int p0, int np,
-                                                              double2 *pbound, double *qout, int full) {{
-    rys_bound_body<C_{tag}>(P, R, tabs_{tag}(), p0, np, pbound, qout, full);
+                                                              double2 *pbound, const int *mol,
+                                                              unsigned long long *qmax, double *qout, int full) {{
+    rys_bound_body<C_{tag}>(P, R, tabs_{tag}(), p0, np, pbound, mol, qmax, qout, full);
 }}
 """
         bound_launch = f"""
 void launch_rys_bound_{tag}(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound,
-                            double *qout, int full, cudaStream_t s) {{
+                            const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s) {{
     if (np <= 0) return;
     rys_prepare_{tag}();
     constexpr int ng = 128 / C_{tag}::G;
-    rys_bound_kernel_{tag}<<<(np + ng - 1) / ng, 128, {smem_block}, s>>>(P, R, p0, np, pbound, qout, full);
+    rys_bound_kernel_{tag}<<<(np + ng - 1) / ng, 128, {smem_block}, s>>>(P, R, p0, np, pbound, mol, qmax, qout,
+                                                                             full);
 }}
 """
     if t["mixed"]:

@@ -14297,142 +14297,4 @@ int occupancy_eri_dddd(int mixed) {
     return n;
 }
 
-// Bounds of the pairs of one class.
-// full == 0 (plan set-up): for every primitive pair k of pair p, from the diagonal primitive
-//   quartet (a_k b_k | a_k b_k):
-//     pbound[k].x = b_k = sqrt(max over components |(a_k b_k|a_k b_k)|)
-//     pbound[k].y = w_k = sqrt(max over the VRR block |[e0|e0]_kk|), e = la..la+lb
-//   By the Schwarz inequality b_k b_l bounds |(a_k b_k|c_l d_l)| and w_k w_l bounds every
-//   entry of the VRR output block [e0|f0] that the HRR combines.
-// full != 0: the contracted bound Q_p = sqrt(max |(ab|ab)|) into qout[p].
-__global__ void __launch_bounds__(128) schwarz_kernel_dddd(PairTab P, BoysTab B, int p0, int np,
-                                                          double2 *pbound, double *qout, int full) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= np) return;
-    const int p = p0 + t;
-    const int4 in = __ldg(&P.info[p]);
-    double res[1296];
-    if (full) {
-        quartet_dddd<double>(P, B, p, p, 0, in.y, 0, in.y, res);
-        double m = 0.0;
-    m = fmax(m, fabs(res[0]));
-    m = fmax(m, fabs(res[37]));
-    m = fmax(m, fabs(res[74]));
-    m = fmax(m, fabs(res[111]));
-    m = fmax(m, fabs(res[148]));
-    m = fmax(m, fabs(res[185]));
-    m = fmax(m, fabs(res[222]));
-    m = fmax(m, fabs(res[259]));
-    m = fmax(m, fabs(res[296]));
-    m = fmax(m, fabs(res[333]));
-    m = fmax(m, fabs(res[370]));
-    m = fmax(m, fabs(res[407]));
-    m = fmax(m, fabs(res[444]));
-    m = fmax(m, fabs(res[481]));
-    m = fmax(m, fabs(res[518]));
-    m = fmax(m, fabs(res[555]));
-    m = fmax(m, fabs(res[592]));
-    m = fmax(m, fabs(res[629]));
-    m = fmax(m, fabs(res[666]));
-    m = fmax(m, fabs(res[703]));
-    m = fmax(m, fabs(res[740]));
-    m = fmax(m, fabs(res[777]));
-    m = fmax(m, fabs(res[814]));
-    m = fmax(m, fabs(res[851]));
-    m = fmax(m, fabs(res[888]));
-    m = fmax(m, fabs(res[925]));
-    m = fmax(m, fabs(res[962]));
-    m = fmax(m, fabs(res[999]));
-    m = fmax(m, fabs(res[1036]));
-    m = fmax(m, fabs(res[1073]));
-    m = fmax(m, fabs(res[1110]));
-    m = fmax(m, fabs(res[1147]));
-    m = fmax(m, fabs(res[1184]));
-    m = fmax(m, fabs(res[1221]));
-    m = fmax(m, fabs(res[1258]));
-    m = fmax(m, fabs(res[1295]));
-        qout[p] = sqrt(m);
-        return;
-    }
-    double acc[961];
-    for (int k = 0; k < in.y; ++k) {
-        quartet_dddd<double>(P, B, p, p, k, k + 1, k, k + 1, res, acc);
-        double m = 0.0, w = 0.0;
-    m = fmax(m, fabs(res[0]));
-    m = fmax(m, fabs(res[37]));
-    m = fmax(m, fabs(res[74]));
-    m = fmax(m, fabs(res[111]));
-    m = fmax(m, fabs(res[148]));
-    m = fmax(m, fabs(res[185]));
-    m = fmax(m, fabs(res[222]));
-    m = fmax(m, fabs(res[259]));
-    m = fmax(m, fabs(res[296]));
-    m = fmax(m, fabs(res[333]));
-    m = fmax(m, fabs(res[370]));
-    m = fmax(m, fabs(res[407]));
-    m = fmax(m, fabs(res[444]));
-    m = fmax(m, fabs(res[481]));
-    m = fmax(m, fabs(res[518]));
-    m = fmax(m, fabs(res[555]));
-    m = fmax(m, fabs(res[592]));
-    m = fmax(m, fabs(res[629]));
-    m = fmax(m, fabs(res[666]));
-    m = fmax(m, fabs(res[703]));
-    m = fmax(m, fabs(res[740]));
-    m = fmax(m, fabs(res[777]));
-    m = fmax(m, fabs(res[814]));
-    m = fmax(m, fabs(res[851]));
-    m = fmax(m, fabs(res[888]));
-    m = fmax(m, fabs(res[925]));
-    m = fmax(m, fabs(res[962]));
-    m = fmax(m, fabs(res[999]));
-    m = fmax(m, fabs(res[1036]));
-    m = fmax(m, fabs(res[1073]));
-    m = fmax(m, fabs(res[1110]));
-    m = fmax(m, fabs(res[1147]));
-    m = fmax(m, fabs(res[1184]));
-    m = fmax(m, fabs(res[1221]));
-    m = fmax(m, fabs(res[1258]));
-    m = fmax(m, fabs(res[1295]));
-        w = fmax(w, fabs(acc[0]));
-        w = fmax(w, fabs(acc[32]));
-        w = fmax(w, fabs(acc[64]));
-        w = fmax(w, fabs(acc[96]));
-        w = fmax(w, fabs(acc[128]));
-        w = fmax(w, fabs(acc[160]));
-        w = fmax(w, fabs(acc[192]));
-        w = fmax(w, fabs(acc[224]));
-        w = fmax(w, fabs(acc[256]));
-        w = fmax(w, fabs(acc[288]));
-        w = fmax(w, fabs(acc[320]));
-        w = fmax(w, fabs(acc[352]));
-        w = fmax(w, fabs(acc[384]));
-        w = fmax(w, fabs(acc[416]));
-        w = fmax(w, fabs(acc[448]));
-        w = fmax(w, fabs(acc[480]));
-        w = fmax(w, fabs(acc[512]));
-        w = fmax(w, fabs(acc[544]));
-        w = fmax(w, fabs(acc[576]));
-        w = fmax(w, fabs(acc[608]));
-        w = fmax(w, fabs(acc[640]));
-        w = fmax(w, fabs(acc[672]));
-        w = fmax(w, fabs(acc[704]));
-        w = fmax(w, fabs(acc[736]));
-        w = fmax(w, fabs(acc[768]));
-        w = fmax(w, fabs(acc[800]));
-        w = fmax(w, fabs(acc[832]));
-        w = fmax(w, fabs(acc[864]));
-        w = fmax(w, fabs(acc[896]));
-        w = fmax(w, fabs(acc[928]));
-        w = fmax(w, fabs(acc[960]));
-        pbound[in.x + k] = make_double2(sqrt(m), sqrt(w));
-    }
-}
-
-void launch_schwarz_dddd(const PairTab &P, const BoysTab &B, int p0, int np, double2 *pbound,
-                          double *qout, int full, cudaStream_t s) {
-    if (np <= 0) return;
-    schwarz_kernel_dddd<<<(np + 127) / 128, 128, 0, s>>>(P, B, p0, np, pbound, qout, full);
-}
-
 }  // namespace molints

@@ -567,15 +567,20 @@ int occupancy_eri_dsds(int mixed) {
 //     pbound[k].y = w_k = sqrt(max over the VRR block |[e0|e0]_kk|), e = la..la+lb
 //   By the Schwarz inequality b_k b_l bounds |(a_k b_k|c_l d_l)| and w_k w_l bounds every
 //   entry of the VRR output block [e0|f0] that the HRR combines.
+//   qmax[mol[p]]: the largest sum of b_k (in list order) over the molecule's pairs, as bits.
 // full != 0: the contracted bound Q_p = sqrt(max |(ab|ab)|) into qout[p].
+// A warp per pair, its lanes over the primitive pairs (one thread per pair, over up to 49 primitive
+// pairs in turn, took 46 us for (ss) on B200).
 __global__ void __launch_bounds__(128) schwarz_kernel_dsds(PairTab P, BoysTab B, int p0, int np,
-                                                          double2 *pbound, double *qout, int full) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+                                                          double2 *pbound, const int *mol,
+                                                          unsigned long long *qmax, double *qout, int full) {
+    const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (t >= np) return;
     const int p = p0 + t;
     const int4 in = __ldg(&P.info[p]);
     double res[36];
     if (full) {
+        if (lane) return;
         quartet_dsds<double>(P, B, p, p, 0, in.y, 0, in.y, res);
         double m = 0.0;
     m = fmax(m, fabs(res[0]));
@@ -587,10 +592,12 @@ __global__ void __launch_bounds__(128) schwarz_kernel_dsds(PairTab P, BoysTab B,
         qout[p] = sqrt(m);
         return;
     }
-    double acc[36];
-    for (int k = 0; k < in.y; ++k) {
-        quartet_dsds<double>(P, B, p, p, k, k + 1, k, k + 1, res, acc);
+    double acc[36], q = 0.0;
+    for (int k0 = 0; k0 < in.y; k0 += 32) {
+        const int k = k0 + lane;
         double m = 0.0, w = 0.0;
+        if (k < in.y) {
+            quartet_dsds<double>(P, B, p, p, k, k + 1, k, k + 1, res, acc);
     m = fmax(m, fabs(res[0]));
     m = fmax(m, fabs(res[7]));
     m = fmax(m, fabs(res[14]));
@@ -603,14 +610,20 @@ __global__ void __launch_bounds__(128) schwarz_kernel_dsds(PairTab P, BoysTab B,
         w = fmax(w, fabs(acc[21]));
         w = fmax(w, fabs(acc[28]));
         w = fmax(w, fabs(acc[35]));
-        pbound[in.x + k] = make_double2(sqrt(m), sqrt(w));
+            m = sqrt(m);
+            pbound[in.x + k] = make_double2(m, sqrt(w));
+        }
+        const int n = min(32, in.y - k0);
+        for (int x = 0; x < n; ++x) q += __shfl_sync(0xffffffffu, m, x);
     }
+    // the sums are >= 0, so their bit patterns order like the values
+    if (lane == 0) atomicMax(&qmax[__ldg(&mol[p])], (unsigned long long)__double_as_longlong(q));
 }
 
 void launch_schwarz_dsds(const PairTab &P, const BoysTab &B, int p0, int np, double2 *pbound,
-                          double *qout, int full, cudaStream_t s) {
+                          const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s) {
     if (np <= 0) return;
-    schwarz_kernel_dsds<<<(np + 127) / 128, 128, 0, s>>>(P, B, p0, np, pbound, qout, full);
+    schwarz_kernel_dsds<<<(np + 3) / 4, 128, 0, s>>>(P, B, p0, np, pbound, mol, qmax, qout, full);
 }
 
 }  // namespace molints

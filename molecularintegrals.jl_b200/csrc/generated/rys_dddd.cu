@@ -313,8 +313,9 @@ __global__ void __launch_bounds__(128) rys_queue_dddd(const EriQueue Q, const Ry
 }
 
 __global__ void __launch_bounds__(128) rys_bound_kernel_dddd(PairTab P, RysTab R, int p0, int np,
-                                                              double2 *pbound, double *qout, int full) {
-    rys_bound_body<C_dddd>(P, R, tabs_dddd(), p0, np, pbound, qout, full);
+                                                              double2 *pbound, const int *mol,
+                                                              unsigned long long *qmax, double *qout, int full) {
+    rys_bound_body<C_dddd>(P, R, tabs_dddd(), p0, np, pbound, mol, qmax, qout, full);
 }
 
 static void rys_prepare_dddd() {
@@ -349,11 +350,12 @@ int occupancy_rys_dddd(int mixed) {
 }
 
 void launch_rys_bound_dddd(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound,
-                            double *qout, int full, cudaStream_t s) {
+                            const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s) {
     if (np <= 0) return;
     rys_prepare_dddd();
     constexpr int ng = 128 / C_dddd::G;
-    rys_bound_kernel_dddd<<<(np + ng - 1) / ng, 128, 78336, s>>>(P, R, p0, np, pbound, qout, full);
+    rys_bound_kernel_dddd<<<(np + ng - 1) / ng, 128, 78336, s>>>(P, R, p0, np, pbound, mol, qmax, qout,
+                                                                             full);
 }
 
 }  // namespace molints

@@ -136,8 +136,9 @@ __global__ void __launch_bounds__(128) rys_queue_dpdp(const EriQueue Q, const Ry
 }
 
 __global__ void __launch_bounds__(128) rys_bound_kernel_dpdp(PairTab P, RysTab R, int p0, int np,
-                                                              double2 *pbound, double *qout, int full) {
-    rys_bound_body<C_dpdp>(P, R, tabs_dpdp(), p0, np, pbound, qout, full);
+                                                              double2 *pbound, const int *mol,
+                                                              unsigned long long *qmax, double *qout, int full) {
+    rys_bound_body<C_dpdp>(P, R, tabs_dpdp(), p0, np, pbound, mol, qmax, qout, full);
 }
 
 static void rys_prepare_dpdp() {
@@ -172,11 +173,12 @@ int occupancy_rys_dpdp(int mixed) {
 }
 
 void launch_rys_bound_dpdp(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound,
-                            double *qout, int full, cudaStream_t s) {
+                            const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s) {
     if (np <= 0) return;
     rys_prepare_dpdp();
     constexpr int ng = 128 / C_dpdp::G;
-    rys_bound_kernel_dpdp<<<(np + ng - 1) / ng, 128, 41472, s>>>(P, R, p0, np, pbound, qout, full);
+    rys_bound_kernel_dpdp<<<(np + ng - 1) / ng, 128, 41472, s>>>(P, R, p0, np, pbound, mol, qmax, qout,
+                                                                             full);
 }
 
 }  // namespace molints

@@ -63,8 +63,9 @@ __global__ void __launch_bounds__(128) rys_queue_dsds(const EriQueue Q, const Ry
 }
 
 __global__ void __launch_bounds__(128) rys_bound_kernel_dsds(PairTab P, RysTab R, int p0, int np,
-                                                              double2 *pbound, double *qout, int full) {
-    rys_bound_body<C_dsds>(P, R, tabs_dsds(), p0, np, pbound, qout, full);
+                                                              double2 *pbound, const int *mol,
+                                                              unsigned long long *qmax, double *qout, int full) {
+    rys_bound_body<C_dsds>(P, R, tabs_dsds(), p0, np, pbound, mol, qmax, qout, full);
 }
 
 static void rys_prepare_dsds() {
@@ -99,11 +100,12 @@ int occupancy_rys_dsds(int mixed) {
 }
 
 void launch_rys_bound_dsds(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound,
-                            double *qout, int full, cudaStream_t s) {
+                            const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s) {
     if (np <= 0) return;
     rys_prepare_dsds();
     constexpr int ng = 128 / C_dsds::G;
-    rys_bound_kernel_dsds<<<(np + ng - 1) / ng, 128, 25920, s>>>(P, R, p0, np, pbound, qout, full);
+    rys_bound_kernel_dsds<<<(np + ng - 1) / ng, 128, 25920, s>>>(P, R, p0, np, pbound, mol, qmax, qout,
+                                                                             full);
 }
 
 }  // namespace molints

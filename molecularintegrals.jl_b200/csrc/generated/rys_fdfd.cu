@@ -482,8 +482,9 @@ __global__ void __launch_bounds__(128) rys_queue_fdfd(const EriQueue Q, const Ry
 }
 
 __global__ void __launch_bounds__(128) rys_bound_kernel_fdfd(PairTab P, RysTab R, int p0, int np,
-                                                              double2 *pbound, double *qout, int full) {
-    rys_bound_body<C_fdfd>(P, R, tabs_fdfd(), p0, np, pbound, qout, full);
+                                                              double2 *pbound, const int *mol,
+                                                              unsigned long long *qmax, double *qout, int full) {
+    rys_bound_body<C_fdfd>(P, R, tabs_fdfd(), p0, np, pbound, mol, qmax, qout, full);
 }
 
 static void rys_prepare_fdfd() {
@@ -518,11 +519,12 @@ int occupancy_rys_fdfd(int mixed) {
 }
 
 void launch_rys_bound_fdfd(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound,
-                            double *qout, int full, cudaStream_t s) {
+                            const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s) {
     if (np <= 0) return;
     rys_prepare_fdfd();
     constexpr int ng = 128 / C_fdfd::G;
-    rys_bound_kernel_fdfd<<<(np + ng - 1) / ng, 128, 103680, s>>>(P, R, p0, np, pbound, qout, full);
+    rys_bound_kernel_fdfd<<<(np + ng - 1) / ng, 128, 103680, s>>>(P, R, p0, np, pbound, mol, qmax, qout,
+                                                                             full);
 }
 
 }  // namespace molints

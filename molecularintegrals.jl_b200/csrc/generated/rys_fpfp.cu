@@ -196,8 +196,9 @@ __global__ void __launch_bounds__(128) rys_queue_fpfp(const EriQueue Q, const Ry
 }
 
 __global__ void __launch_bounds__(128) rys_bound_kernel_fpfp(PairTab P, RysTab R, int p0, int np,
-                                                              double2 *pbound, double *qout, int full) {
-    rys_bound_body<C_fpfp>(P, R, tabs_fpfp(), p0, np, pbound, qout, full);
+                                                              double2 *pbound, const int *mol,
+                                                              unsigned long long *qmax, double *qout, int full) {
+    rys_bound_body<C_fpfp>(P, R, tabs_fpfp(), p0, np, pbound, mol, qmax, qout, full);
 }
 
 static void rys_prepare_fpfp() {
@@ -232,11 +233,12 @@ int occupancy_rys_fpfp(int mixed) {
 }
 
 void launch_rys_bound_fpfp(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound,
-                            double *qout, int full, cudaStream_t s) {
+                            const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s) {
     if (np <= 0) return;
     rys_prepare_fpfp();
     constexpr int ng = 128 / C_fpfp::G;
-    rys_bound_kernel_fpfp<<<(np + ng - 1) / ng, 128, 53760, s>>>(P, R, p0, np, pbound, qout, full);
+    rys_bound_kernel_fpfp<<<(np + ng - 1) / ng, 128, 53760, s>>>(P, R, p0, np, pbound, mol, qmax, qout,
+                                                                             full);
 }
 
 }  // namespace molints

@@ -76,8 +76,9 @@ __global__ void __launch_bounds__(128) rys_queue_fsfs(const EriQueue Q, const Ry
 }
 
 __global__ void __launch_bounds__(128) rys_bound_kernel_fsfs(PairTab P, RysTab R, int p0, int np,
-                                                              double2 *pbound, double *qout, int full) {
-    rys_bound_body<C_fsfs>(P, R, tabs_fsfs(), p0, np, pbound, qout, full);
+                                                              double2 *pbound, const int *mol,
+                                                              unsigned long long *qmax, double *qout, int full) {
+    rys_bound_body<C_fsfs>(P, R, tabs_fsfs(), p0, np, pbound, mol, qmax, qout, full);
 }
 
 static void rys_prepare_fsfs() {
@@ -112,11 +113,12 @@ int occupancy_rys_fsfs(int mixed) {
 }
 
 void launch_rys_bound_fsfs(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound,
-                            double *qout, int full, cudaStream_t s) {
+                            const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s) {
     if (np <= 0) return;
     rys_prepare_fsfs();
     constexpr int ng = 128 / C_fsfs::G;
-    rys_bound_kernel_fsfs<<<(np + ng - 1) / ng, 128, 37632, s>>>(P, R, p0, np, pbound, qout, full);
+    rys_bound_kernel_fsfs<<<(np + ng - 1) / ng, 128, 37632, s>>>(P, R, p0, np, pbound, mol, qmax, qout,
+                                                                             full);
 }
 
 }  // namespace molints

@@ -91,8 +91,9 @@ __global__ void __launch_bounds__(128) rys_queue_pppp(const EriQueue Q, const Ry
 }
 
 __global__ void __launch_bounds__(128) rys_bound_kernel_pppp(PairTab P, RysTab R, int p0, int np,
-                                                              double2 *pbound, double *qout, int full) {
-    rys_bound_body<C_pppp>(P, R, tabs_pppp(), p0, np, pbound, qout, full);
+                                                              double2 *pbound, const int *mol,
+                                                              unsigned long long *qmax, double *qout, int full) {
+    rys_bound_body<C_pppp>(P, R, tabs_pppp(), p0, np, pbound, mol, qmax, qout, full);
 }
 
 static void rys_prepare_pppp() {
@@ -127,11 +128,12 @@ int occupancy_rys_pppp(int mixed) {
 }
 
 void launch_rys_bound_pppp(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound,
-                            double *qout, int full, cudaStream_t s) {
+                            const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s) {
     if (np <= 0) return;
     rys_prepare_pppp();
     constexpr int ng = 128 / C_pppp::G;
-    rys_bound_kernel_pppp<<<(np + ng - 1) / ng, 128, 23328, s>>>(P, R, p0, np, pbound, qout, full);
+    rys_bound_kernel_pppp<<<(np + ng - 1) / ng, 128, 23328, s>>>(P, R, p0, np, pbound, mol, qmax, qout,
+                                                                             full);
 }
 
 }  // namespace molints

@@ -62,7 +62,10 @@ struct molints_ctx {
     // kSideTwoPhase.  On B200, us per execute with 6 / 16 / 24 streams: 8 polarised atoms 99 / 87 /
     // 78, 11 atoms with f shells 340 / 277 / 254, 15 polarised atoms 324 / 329 / 335, a batch of
     // 1.17e9 integrals 7025 / 7139 / 7253.
-    static constexpr int kSide = 24, kSideTwoPhase = 6;
+    // Executes that are not captured take kSideEager unless they launch many kernels (f shells): each
+    // stream costs three calls of the host (8 polarised atoms, 22 launches, us of host and total
+    // with 24 / 8 streams: 118, 128 / 112, 127; 11 atoms with f shells, 57 launches: 296, 308 / 265, 373).
+    static constexpr int kSide = 24, kSideEager = 8, kSideTwoPhase = 6;
     cudaStream_t side[kSide] = {};
     cudaEvent_t fork = nullptr, join[kSide] = {};
     int num_sms = 0;
@@ -107,7 +110,8 @@ struct molints_plan {
     std::vector<int> pair_ref;         // canonical pair -> reference pair index i(i+1)/2+j
     std::vector<int> npp_h;            // kept primitive pairs per shell pair
     std::vector<double2> bnd_h;        // (Qabs, R) per shell pair
-    // device buffers
+    // device buffers: slab holds all from here to g_units but the chunks and qcon
+    char *slab = nullptr;
     double *sh_xyz = nullptr, *expn = nullptr, *ncoef = nullptr;
     int *sh_poff = nullptr;
     int2 *pair_ab = nullptr;
@@ -204,11 +208,15 @@ double boys_series(int m, double T) {
     return (double)(expl(-t) * sum);
 }
 
-int pair_class_of(int la, int lb) {
-    for (int c = 0; c < kNumPairClasses; ++c)
-        if (kPairClassLa[c] == la && kPairClassLb[c] == lb) return c;
-    return -1;
-}
+// Pair class of an oriented pair of shells up to f (-1: none).
+struct PairClassOf {
+    signed char c[kLmax + 1][kLmax + 1];
+    PairClassOf() {
+        std::memset(c, -1, sizeof c);
+        for (int k = 0; k < kNumPairClasses; ++k) c[kPairClassLa[k]][kPairClassLb[k]] = (signed char)k;
+    }
+};
+const PairClassOf kPairClassOf;
 
 // Stable LSD radix order of keys[0..n) over their low `bits` bits (8-bit digits): the
 // permutation position -> index, equal keys in index order.  O(n bits / 8).
@@ -316,26 +324,33 @@ namespace molints {
 // norm (2a/pi)^(3/4) (4a)^(L/2) x the contracted norm 1/sqrt(S), S = sum_ij c_i c_j
 // (2 sqrt(a_i a_j) / (a_i + a_j))^(L + 3/2) the self-overlap of the shell's function (PGBF/CGBF
 // normalize!, src/Basis.jl:42-83; the component factor 1/sqrt((2I-1)!!(2J-1)!!(2K-1)!!) is
-// applied by the ERI kernels).  One thread per shell; a shell whose S is not positive sets
-// *bad (the plan is refused).
+// applied by the ERI kernels).  A warp per shell, its lanes over the terms of S, which are added in
+// order (one thread per shell, K^2 powers in turn, took 38 us on B200); a shell whose S is not
+// positive sets *bad (the plan is refused).
 __global__ void normalise_shells_kernel(int ns, const int *__restrict__ L, const int *__restrict__ K,
                                         const int *__restrict__ poff, const double *__restrict__ expn,
                                         double *__restrict__ coef, int *__restrict__ bad) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (g >= ns) return;
     const int Ls = L[g], Ks = K[g], p0 = poff[g];
     double S = 0.0;
-    for (int i = 0; i < Ks; ++i)
-        for (int j = 0; j < Ks; ++j) {
+    for (int t0 = 0; t0 < Ks * Ks; t0 += 32) {
+        const int t = t0 + lane, n = min(32, Ks * Ks - t0);
+        double v = 0.0;
+        if (lane < n) {
+            const int i = t / Ks, j = t - i * Ks;
             const double x = expn[p0 + i], y = expn[p0 + j];
-            S += coef[p0 + i] * coef[p0 + j] * pow(2.0 * sqrt(x * y) / (x + y), Ls + 1.5);
+            v = coef[p0 + i] * coef[p0 + j] * pow(2.0 * sqrt(x * y) / (x + y), Ls + 1.5);
         }
+        for (int k = 0; k < n; ++k) S += __shfl_sync(0xffffffffu, v, k);
+    }
     if (!(S > 0.0)) {
-        atomicExch(bad, 1);
+        if (lane == 0) atomicExch(bad, 1);
         return;
     }
     const double cn = 1.0 / sqrt(S);
-    for (int i = 0; i < Ks; ++i) {
+    __syncwarp();
+    for (int i = lane; i < Ks; i += 32) {
         const double a = expn[p0 + i];
         coef[p0 + i] *= cn * pow(2.0 * a / 3.14159265358979323846, 0.75) * pow(4.0 * a, 0.5 * Ls);
     }
@@ -343,7 +358,8 @@ __global__ void normalise_shells_kernel(int ns, const int *__restrict__ L, const
 
 __global__ void build_pairs_kernel(int npair, const int2 *__restrict__ pair_ab,
                                    const int4 *__restrict__ info, const int *__restrict__ pp_src,
-                                   const double *__restrict__ xyz, const int *__restrict__ poff,
+                                   const int *__restrict__ nprim, const double *__restrict__ xyz,
+                                   const int *__restrict__ poff,
                                    const double *__restrict__ expn,
                                    const double *__restrict__ ncoef, double c0,
                                    const double *__restrict__ pb,
@@ -364,7 +380,7 @@ __global__ void build_pairs_kernel(int npair, const int2 *__restrict__ pair_ab,
     const double rab2 = ABx * ABx + ABy * ABy + ABz * ABz;
     const int pa0 = poff[ab.x], pb0 = poff[ab.y];
     for (int k = in.x + lane; k < in.x + in.y; k += 32) {
-        const int src = pp_src[k];
+        const int src = pp_src ? pp_src[k] : prim_src(k - in.x, nprim[ab.y]);  // (every primitive pair)
         const double a = expn[pa0 + (src >> 8)], ca = ncoef[pa0 + (src >> 8)];
         const double b = expn[pb0 + (src & 255)], cb = ncoef[pb0 + (src & 255)];
         const double zeta = a + b, ooz = 1.0 / zeta;
@@ -760,7 +776,7 @@ void launch_build_pairs(int npair, const int2 *pair_ab, const int4 *info, const 
                         const double *xyz, const int *poff, const double *expn,
                         const double *ncoef, PrimPair *pp, double4 *geo, cudaStream_t s) {
     if (npair <= 0) return;
-    build_pairs_kernel<<<build_pairs_blocks(npair), 128, 0, s>>>(npair, pair_ab, info, pp_src, xyz, poff,
+    build_pairs_kernel<<<build_pairs_blocks(npair), 128, 0, s>>>(npair, pair_ab, info, pp_src, nullptr, xyz, poff,
                                                           expn, ncoef, std::sqrt(2.0) * std::pow(M_PI, 1.25),
                                                           nullptr, pp, geo, nullptr, 0);
 }
@@ -1091,10 +1107,7 @@ static void plan_release_device(molints_plan *p) {
     p->gexec = nullptr;
     for (cudaEvent_t e : p->prof_ev) cudaEventDestroy(e);
     p->prof_ev.clear();
-    void *bufs[] = {p->sh_xyz, p->expn, p->ncoef, p->sh_poff, p->pair_ab, p->info, p->pp_src, p->pbk,
-                    p->geo, p->pp, p->bnd, p->chunks, p->counters, p->mol_out, p->qcon,
-                    p->chunk_slot, p->g_fn, p->g_pair, p->g_region, p->g_mol, p->g_col, p->g_list, p->g_colq, p->g_index, p->g_end, p->g_nlive,
-                    p->g_units, p->gq, p->gq_mol, p->sh_L, p->sh_K, p->sh_fn};
+    void *bufs[] = {p->slab, p->chunks, p->chunk_slot, p->qcon, p->gq, p->gq_mol, p->sh_fn};
     for (void *b : bufs) dev_free(p->ctx, b);
     p->ctx->held -= p->bytes;
     p->ctx = nullptr;
@@ -1371,7 +1384,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
                 }
                 if (g_ij) continue;
                 if (!a_first(a, bb)) std::swap(a, bb);
-                pr.push_back({pair_class_of(L[a], L[bb]), m, K[a] * K[bb], a, bb, i * (i + 1) / 2 + j, i});
+                pr.push_back({kPairClassOf.c[L[a]][L[bb]], m, K[a] * K[bb], a, bb, i * (i + 1) / 2 + j, i});
             }
     }
     p->n_gunits = (int64_t)gq_h.size();
@@ -1578,9 +1591,16 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     const size_t t_ab1 = tv.take<int2>(npair), t_info1 = tv.take<int4>(npair), t_rec1 = tv.take<int4>(npair);
     const size_t t_seg1 = tv.take<int>(npair), t_mol1 = tv.take<int>(npair);
     const size_t t_cm = tv.take<int>(cm_start.size()), t_lane = tv.take<double>(nmol);
+    const size_t t_units = tv.take<int4>(tp ? npe_all : 0);
     const size_t up_bytes = tv.at;
-    const size_t t_src1 = tv.take<int>(nall);
-    const size_t t_pbound = tv.take<double2>(nall), t_qmax = tv.take<unsigned long long>(nmol);
+    // cleared before the build: the molecules' Qabs bounds and the summary that is read back
+    // (class-pair chunk offsets, the count of pairs without kept primitive pairs, class-pair costs,
+    // kept primitive pairs, bad-shell flag)
+    const size_t t_qmax = tv.take<unsigned long long>(nmol);
+    const size_t t_sum = tv.take<long long>(kNumClassPairs + 2), t_ccost = tv.take<double>(kNumClassPairs);
+    const size_t t_nkept = tv.take<long long>(1), t_bad = tv.take<int>(1);
+    const size_t clear_end = tv.at;
+    const size_t t_pbound = tv.take<double2>(nall);
     const size_t t_npp1 = tv.take<int>(npair), t_bnd1 = tv.take<double2>(npair);
     const size_t t_key1 = tv.take<unsigned long long>(npair), t_key2 = tv.take<unsigned long long>(npair);
     const size_t t_idx1 = tv.take<int>(npair), t_idx2 = tv.take<int>(npair);
@@ -1588,21 +1608,31 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     const size_t t_ms = tv.take<int>(npair);
     const size_t t_cnt = tv.take<long long>((size_t)n_items + 1), t_cost = tv.take<double>(n_items);
     const size_t t_off = tv.take<long long>((size_t)n_items + 1);
-    const size_t t_sum = tv.take<long long>(kNumClassPairs + 2), t_ccost = tv.take<double>(kNumClassPairs);
     const size_t cub_bytes = std::max(plan_build_temp_bytes(npair), queue_count_temp_bytes(n_items));
-    const size_t t_cub = tv.take<char>(cub_bytes), t_units = tv.take<int4>(tp ? npe_all : 0);
+    const size_t t_cub = tv.take<char>(cub_bytes);
+    // the plan's buffers, one allocation; what is uploaded comes first, laid out as in the stage
+    const int nc2 = kNumPairClasses * kNumPairClasses;
+    Carve pv;
+    const size_t o_xyz = pv.take<double>(3 * (size_t)ns), o_expn = pv.take<double>(nprim);
+    const size_t o_coef = pv.take<double>(nprim), o_poff = pv.take<int>(ns), o_L = pv.take<int>(ns);
+    const size_t o_K = pv.take<int>(ns), o_mol = pv.take<long long>(nmol);
+    const size_t o_greg = pv.take<long long>(tp ? region_h.size() : 0), o_gfn = pv.take<int2>(tp ? nfn_all : 0);
+    const size_t o_gmol = pv.take<long long>(tp ? (size_t)nmol * 4 : 0);
+    const size_t plan_up = pv.at;
+    // (pair_ab, info and bnd together: plan_host_tables reads them back in one copy)
+    const size_t d_ab = pv.take<int2>(npair), d_info = pv.take<int4>(npair), d_bnd = pv.take<double2>(npair);
+    const size_t d_geo = pv.take<double4>(npair), d_src = pv.take<int>(nall), d_pbk = pv.take<double>(nall);
+    // kept primitive pairs: at most nall (the count is known on the device only)
+    const size_t d_pp = pv.take<PrimPair>(nall);
+    const size_t d_counters = pv.take<int>((size_t)nc2 + 2);  // + the gather's two or the g kernel's
+    const int64_t nrows_tp = tp ? nrows_all : 0, npe_tp = tp ? npe_all : 0;
+    const size_t d_gpair = pv.take<int>(npe_tp), d_gcol = pv.take<int2>(nrows_tp), d_glist = pv.take<int4>(nrows_tp);
+    const size_t d_gcolq = pv.take<double>(opts.screen_cutoff > 0.0 ? nrows_tp : 0);
+    const size_t d_gindex = pv.take<int>(tp ? (nrows_all >> kGatherIndexShift) + nmol + 1 : 0);
+    const size_t d_gend = pv.take<int>(tp ? nmol : 0), d_gnlive = pv.take<int>(1), d_gunits = pv.take<int4>(npe_tp);
     Carve sv;
-    // read back: class-pair chunk offsets and the count of pairs without kept primitive pairs,
-    // class-pair costs, kept primitive pairs, bad-shell flag
-    const size_t o_sum = sv.take<long long>(kNumClassPairs + 2), o_ccost = sv.take<double>(kNumClassPairs);
-    const size_t o_nkept = sv.take<long long>(1), o_bad = sv.take<int>(1);
-    const size_t o_up = sv.take<char>(up_bytes);
-    const size_t o_xyz = sv.take<double>(3 * (size_t)ns), o_expn = sv.take<double>(nprim);
-    const size_t o_coef = sv.take<double>(nprim), o_poff = sv.take<int>(ns), o_L = sv.take<int>(ns);
-    const size_t o_K = sv.take<int>(ns), o_mol = sv.take<long long>(nmol);
-    const size_t o_greg = sv.take<long long>(tp ? region_h.size() : 0), o_gfn = sv.take<int2>(tp ? nfn_all : 0);
-    const size_t o_gmol = sv.take<long long>(tp ? (size_t)nmol * 4 : 0);
-    const size_t o_gunits = sv.take<int4>(tp ? npe_all : 0);
+    const size_t o_sum = sv.take<char>(t_bad + sizeof(int) - t_sum), o_up = sv.take<char>(up_bytes);
+    const size_t o_plan = sv.take<char>(plan_up);
     int rc = ctx_stage(ctx, sv.at);
     if (rc) { plan_free(p); return rc; }
     char *stage = ctx->stage;
@@ -1611,7 +1641,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
         int2 *ab1 = reinterpret_cast<int2 *>(up + t_ab1);
         int4 *info1 = reinterpret_cast<int4 *>(up + t_info1), *rec1 = reinterpret_cast<int4 *>(up + t_rec1);
         int *seg1 = reinterpret_cast<int *>(up + t_seg1), *mol1 = reinterpret_cast<int *>(up + t_mol1);
-        int off = 0;  // the primitive pairs themselves are listed on the device (plan_stage1_src)
+        int off = 0;  // (the kernels number a pair's primitive pairs themselves: prim_src)
         for (int k = 0; k < npair; ++k) {
             const PairRec &r = pr[k];
             const int m = r.mol;
@@ -1631,21 +1661,21 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
         for (const PairRec &r : pr) lane[r.mol] += r.npp;
         for (int m = 0; m < nmol; ++m) lane[m] = molecule_lane_cost(lane[m], ctx->sched.lane_cost);
     }
-    std::memcpy(stage + o_xyz, xyz.data(), 3 * (size_t)ns * sizeof(double));
-    std::memcpy(stage + o_expn, expn.data(), (size_t)nprim * sizeof(double));
-    std::memcpy(stage + o_coef, ncoef.data(), (size_t)nprim * sizeof(double));
-    std::memcpy(stage + o_poff, poff.data(), (size_t)ns * sizeof(int));
-    std::memcpy(stage + o_L, L.data(), (size_t)ns * sizeof(int));
-    std::memcpy(stage + o_K, K.data(), (size_t)ns * sizeof(int));
+    std::memcpy(stage + o_plan + o_xyz, xyz.data(), 3 * (size_t)ns * sizeof(double));
+    std::memcpy(stage + o_plan + o_expn, expn.data(), (size_t)nprim * sizeof(double));
+    std::memcpy(stage + o_plan + o_coef, ncoef.data(), (size_t)nprim * sizeof(double));
+    std::memcpy(stage + o_plan + o_poff, poff.data(), (size_t)ns * sizeof(int));
+    std::memcpy(stage + o_plan + o_L, L.data(), (size_t)ns * sizeof(int));
+    std::memcpy(stage + o_plan + o_K, K.data(), (size_t)ns * sizeof(int));
     {
-        long long *mol_out_ll = reinterpret_cast<long long *>(stage + o_mol);
+        long long *mol_out_ll = reinterpret_cast<long long *>(stage + o_plan + o_mol);
         mol_out_ll[0] = 0;
         for (int m = 0; m < nmol; ++m) mol_out_ll[m] = (long long)p->mol_out_h[m];
     }
     if (tp) {
-        std::memcpy(stage + o_greg, region_h.data(), region_h.size() * sizeof(long long));
-        int2 *gfn = reinterpret_cast<int2 *>(stage + o_gfn);
-        long long *gmol = reinterpret_cast<long long *>(stage + o_gmol);
+        std::memcpy(stage + o_plan + o_greg, region_h.data(), region_h.size() * sizeof(long long));
+        int2 *gfn = reinterpret_cast<int2 *>(stage + o_plan + o_gfn);
+        long long *gmol = reinterpret_cast<long long *>(stage + o_plan + o_gmol);
         long long cbase = 0, pbase = 0;
         for (int m = 0, fb = 0; m < nmol; ++m) {
             for (int sl = 0; sl < bases[m].nshell; ++sl) {
@@ -1662,7 +1692,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
         }
         // gather units: every shell pair I >= J of every molecule, heaviest first (rows x the
         // last row's columns), so that the big pairs do not finish last
-        int4 *gu = reinterpret_cast<int4 *>(stage + o_gunits);
+        int4 *gu = reinterpret_cast<int4 *>(stage + o_up + t_units);
         std::vector<std::pair<double, int64_t>> wk;
         wk.reserve((size_t)npe_all);
         std::vector<int4> u_h;
@@ -1694,37 +1724,37 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     t_phase = clk::now();
 
     // ---- device: plan buffers, uploads, normalisation, bound pass, then the device build
-    const int nc2 = kNumPairClasses * kNumPairClasses;
-    rc = rc ? rc : dev_alloc(ctx, &p->sh_xyz, (size_t)3 * ns, &p->bytes);
-    rc = rc ? rc : dev_alloc(ctx, &p->expn, (size_t)nprim, &p->bytes);
-    rc = rc ? rc : dev_alloc(ctx, &p->ncoef, (size_t)nprim, &p->bytes);
-    rc = rc ? rc : dev_alloc(ctx, &p->sh_poff, (size_t)ns, &p->bytes);
-    rc = rc ? rc : dev_alloc(ctx, &p->sh_L, (size_t)ns, &p->bytes);
-    rc = rc ? rc : dev_alloc(ctx, &p->sh_K, (size_t)ns, &p->bytes);
-    rc = rc ? rc : dev_alloc(ctx, &p->pair_ab, (size_t)npair, &p->bytes);
-    rc = rc ? rc : dev_alloc(ctx, &p->info, (size_t)npair, &p->bytes);
-    rc = rc ? rc : dev_alloc(ctx, &p->geo, (size_t)npair, &p->bytes);
-    rc = rc ? rc : dev_alloc(ctx, &p->bnd, (size_t)npair, &p->bytes);
-    // kept primitive pairs: at most nall (the count is known on the device only)
-    rc = rc ? rc : dev_alloc(ctx, &p->pp_src, (size_t)nall, &p->bytes);
-    rc = rc ? rc : dev_alloc(ctx, &p->pbk, (size_t)nall, &p->bytes);
-    rc = rc ? rc : dev_alloc(ctx, &p->pp, (size_t)nall, &p->bytes);
-    rc = rc ? rc : dev_alloc(ctx, &p->counters, (size_t)nc2 + 2, &p->bytes);  // + the gather's two or the g kernel's
-    rc = rc ? rc : dev_alloc(ctx, &p->mol_out, (size_t)std::max(nmol, 1), &p->bytes);
-    if (tp) {
-        rc = rc ? rc : dev_alloc(ctx, &p->g_fn, (size_t)std::max<int64_t>(nfn_all, 1), &p->bytes);
-        rc = rc ? rc : dev_alloc(ctx, &p->g_pair, (size_t)std::max<int64_t>(npe_all, 1), &p->bytes);
-        rc = rc ? rc : dev_alloc(ctx, &p->g_region, region_h.size(), &p->bytes);
-        rc = rc ? rc : dev_alloc(ctx, &p->g_mol, (size_t)nmol * 4, &p->bytes);
-        rc = rc ? rc : dev_alloc(ctx, &p->g_col, (size_t)std::max<int64_t>(nrows_all, 1), &p->bytes);
-        rc = rc ? rc : dev_alloc(ctx, &p->g_list, (size_t)std::max<int64_t>(nrows_all, 1), &p->bytes);
-        rc = rc ? rc : dev_alloc(ctx, &p->g_index, (size_t)(nrows_all >> kGatherIndexShift) + nmol + 1, &p->bytes);
-        rc = rc ? rc : dev_alloc(ctx, &p->g_nlive, 1, &p->bytes);
-        rc = rc ? rc : dev_alloc(ctx, &p->g_end, (size_t)std::max(nmol, 1), &p->bytes);
-        if (opts.screen_cutoff > 0.0) {
-            rc = rc ? rc : dev_alloc(ctx, &p->g_colq, (size_t)std::max<int64_t>(nrows_all, 1), &p->bytes);
+    rc = dev_alloc(ctx, &p->slab, pv.at, &p->bytes);
+    if (!rc) {
+        char *d = p->slab;
+        p->sh_xyz = reinterpret_cast<double *>(d + o_xyz);
+        p->expn = reinterpret_cast<double *>(d + o_expn);
+        p->ncoef = reinterpret_cast<double *>(d + o_coef);
+        p->sh_poff = reinterpret_cast<int *>(d + o_poff);
+        p->sh_L = reinterpret_cast<int *>(d + o_L);
+        p->sh_K = reinterpret_cast<int *>(d + o_K);
+        p->mol_out = reinterpret_cast<long long *>(d + o_mol);
+        p->pair_ab = reinterpret_cast<int2 *>(d + d_ab);
+        p->info = reinterpret_cast<int4 *>(d + d_info);
+        p->bnd = reinterpret_cast<double2 *>(d + d_bnd);
+        p->geo = reinterpret_cast<double4 *>(d + d_geo);
+        p->pp_src = reinterpret_cast<int *>(d + d_src);
+        p->pbk = reinterpret_cast<double *>(d + d_pbk);
+        p->pp = reinterpret_cast<PrimPair *>(d + d_pp);
+        p->counters = reinterpret_cast<int *>(d + d_counters);
+        if (tp) {
+            p->g_region = reinterpret_cast<long long *>(d + o_greg);
+            p->g_fn = reinterpret_cast<int2 *>(d + o_gfn);
+            p->g_mol = reinterpret_cast<long long *>(d + o_gmol);
+            p->g_pair = reinterpret_cast<int *>(d + d_gpair);
+            p->g_col = reinterpret_cast<int2 *>(d + d_gcol);
+            p->g_list = reinterpret_cast<int4 *>(d + d_glist);
+            p->g_colq = opts.screen_cutoff > 0.0 ? reinterpret_cast<double *>(d + d_gcolq) : nullptr;
+            p->g_index = reinterpret_cast<int *>(d + d_gindex);
+            p->g_end = reinterpret_cast<int *>(d + d_gend);
+            p->g_nlive = reinterpret_cast<int *>(d + d_gnlive);
+            p->g_units = reinterpret_cast<int4 *>(d + d_gunits);
         }
-        rc = rc ? rc : dev_alloc(ctx, &p->g_units, (size_t)std::max<int64_t>(npe_all, 1), &p->bytes);
     }
     int64_t temp_tally = 0;
     char *tmp = nullptr;
@@ -1737,34 +1767,17 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     };
     if (rc) { release_temp(); plan_free(p); return rc; }
     cudaStream_t s = ctx->stream;
-    auto h2d = [&](void *dst, size_t off, size_t bytes) {
-        return bytes ? cudaMemcpyAsync(dst, stage + off, bytes, cudaMemcpyHostToDevice, s) : cudaSuccess;
-    };
-    if ((e = h2d(tmp, o_up, up_bytes)) ||
-        (e = h2d(p->sh_xyz, o_xyz, 3 * (size_t)ns * sizeof(double))) ||
-        (e = h2d(p->expn, o_expn, (size_t)nprim * sizeof(double))) ||
-        (e = h2d(p->ncoef, o_coef, (size_t)nprim * sizeof(double))) ||
-        (e = h2d(p->sh_poff, o_poff, (size_t)ns * sizeof(int))) ||
-        (e = h2d(p->sh_L, o_L, (size_t)ns * sizeof(int))) ||
-        (e = h2d(p->sh_K, o_K, (size_t)ns * sizeof(int))) ||
-        (e = h2d(p->mol_out, o_mol, (size_t)nmol * sizeof(long long))) ||
-        (tp && ((e = h2d(p->g_region, o_greg, region_h.size() * sizeof(long long))) ||
-                (e = h2d(p->g_fn, o_gfn, (size_t)nfn_all * sizeof(int2))) ||
-                (e = h2d(p->g_mol, o_gmol, (size_t)nmol * 4 * sizeof(long long))) ||
-                (e = h2d(tmp + t_units, o_gunits, (size_t)npe_all * sizeof(int4))))) ||
-        (e = cudaMemsetAsync(p->counters + nc2, 0, sizeof(int), s)) ||
-        (e = cudaMemsetAsync(tmp + t_qmax, 0, (size_t)std::max(nmol, 1) * sizeof(unsigned long long), s)) ||
-        (e = cudaMemsetAsync(tmp + t_sum, 0, (kNumClassPairs + 2) * sizeof(long long), s)) ||
-        (e = cudaMemsetAsync(tmp + t_ccost, 0, kNumClassPairs * sizeof(double), s)) ||
-        (e = cudaMemsetAsync(tmp + t_prefix, 0, sizeof(long long), s))) {
+    if ((e = cudaMemcpyAsync(p->slab, stage + o_plan, plan_up, cudaMemcpyHostToDevice, s)) ||
+        (e = cudaMemcpyAsync(tmp, stage + o_up, up_bytes, cudaMemcpyHostToDevice, s)) ||
+        (e = cudaMemsetAsync(tmp + t_qmax, 0, clear_end - t_qmax, s))) {
         release_temp(); plan_free(p);
         return cuda_fail(ctx, e, "plan_create upload");
     }
     // the raw coefficients become normalised ones in place; a shell with no positive
-    // self-overlap flags counters[nc2] (read back with the summary)
+    // self-overlap sets the flag that is read back with the summary
     if (ns > 0)
-        normalise_shells_kernel<<<(ns + 127) / 128, 128, 0, s>>>(ns, p->sh_L, p->sh_K, p->sh_poff, p->expn,
-                                                                 p->ncoef, p->counters + nc2);
+        normalise_shells_kernel<<<(ns + 3) / 4, 128, 0, s>>>(ns, p->sh_L, p->sh_K, p->sh_poff, p->expn, p->ncoef,
+                                                             reinterpret_cast<int *>(tmp + t_bad));
     PlanBuildArgs A{};
     A.npair = npair;
     A.nall = (int)nall;
@@ -1772,12 +1785,13 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     A.screen_sort = S.screen_sort;
     A.ab1 = reinterpret_cast<const int2 *>(tmp + t_ab1);
     A.info1 = reinterpret_cast<const int4 *>(tmp + t_info1);
-    A.src1 = reinterpret_cast<const int *>(tmp + t_src1);
+    for (int k = 0; k < npair; ++k) A.maxnpp = std::max(A.maxnpp, pr[k].npp);
     A.rec1 = reinterpret_cast<const int4 *>(tmp + t_rec1);
     A.seg1 = reinterpret_cast<const int *>(tmp + t_seg1);
     A.pbound = reinterpret_cast<const double2 *>(tmp + t_pbound);
     A.xyz = p->sh_xyz;
     A.sh_L = p->sh_L;
+    A.sh_K = p->sh_K;
     A.qmax = reinterpret_cast<unsigned long long *>(tmp + t_qmax);
     A.n_zero = reinterpret_cast<unsigned long long *>(tmp + t_sum) + kNumClassPairs + 1;
     A.npp1 = reinterpret_cast<int *>(tmp + t_npp1);
@@ -1811,22 +1825,36 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     QA.off = reinterpret_cast<long long *>(tmp + t_off);
     QA.summary = reinterpret_cast<long long *>(tmp + t_sum);
     QA.class_cost = reinterpret_cast<double *>(tmp + t_ccost);
+    QA.nkept = reinterpret_cast<long long *>(tmp + t_nkept);
+    QA.npair = npair;
     if (npair > 0) {
         const double c0 = std::sqrt(2.0) * std::pow(M_PI, 1.25);
-        if ((e = plan_stage1_src(npair, A.ab1, A.info1, p->sh_K, const_cast<int *>(A.src1), s))) {
-            release_temp(); plan_free(p);
-            return cuda_fail(ctx, e, "plan_create pair list");
-        }
-        build_pairs_kernel<<<build_pairs_blocks(npair), 128, 0, s>>>(npair, A.ab1, A.info1, A.src1, p->sh_xyz,
-                                                                     p->sh_poff, p->expn, p->ncoef, c0, nullptr,
-                                                                     p->pp, p->geo, nullptr, 0);
+        build_pairs_kernel<<<build_pairs_blocks(npair), 128, 0, s>>>(npair, A.ab1, A.info1, nullptr, p->sh_K,
+                                                                     p->sh_xyz, p->sh_poff, p->expn, p->ncoef, c0,
+                                                                     nullptr, p->pp, p->geo, nullptr, 0);
+        // the bound pass: a kernel per pair class, the first on the stream itself and the others beside it
         PairTab P1{A.info1, p->geo, p->pp, p->bnd};
         BoysTab Bt = boys_of(ctx, opts.boys);
         double2 *pbound = reinterpret_cast<double2 *>(tmp + t_pbound);
-        for (int c = 0; c < kNumPairClasses; ++c) {
+        unsigned long long *qmax = reinterpret_cast<unsigned long long *>(tmp + t_qmax);
+        int nk = 0;
+        for (int c = 0; c < kNumPairClasses && !e; ++c) {
             const int n = cls_start[c + 1] - cls_start[c];
-            if (kSchwarzLaunchers[c]) kSchwarzLaunchers[c](P1, Bt, cls_start[c], n, pbound, nullptr, 0, s);
-            else kRysBoundLaunchers[c](P1, ctx->rys, cls_start[c], n, pbound, nullptr, 0, s);
+            if (n == 0) continue;
+            cudaStream_t st = nk ? ctx->side[nk - 1] : s;
+            if (nk == 0) e = cudaEventRecord(ctx->fork, s);
+            if (nk && !e) e = cudaStreamWaitEvent(st, ctx->fork, 0);
+            if (kSchwarzLaunchers[c]) kSchwarzLaunchers[c](P1, Bt, cls_start[c], n, pbound, QA.mol, qmax, nullptr, 0, st);
+            else kRysBoundLaunchers[c](P1, ctx->rys, cls_start[c], n, pbound, QA.mol, qmax, nullptr, 0, st);
+            if (nk && !e) e = cudaEventRecord(ctx->join[nk - 1], st);
+            ++nk;
+        }
+        for (int k = 1; k < nk && !e; ++k) e = cudaStreamWaitEvent(s, ctx->join[k - 1], 0);
+        if (e) {
+            cudaStreamSynchronize(s);  // the side streams' kernels use the buffers released here
+            for (int k = 1; k < nk; ++k) cudaStreamSynchronize(ctx->side[k - 1]);
+            release_temp(); plan_free(p);
+            return cuda_fail(ctx, e, "plan_create bound pass");
         }
         if ((e = cudaGetLastError()) || (e = plan_build_pairs(A, tmp + t_cub, cub_bytes, s)) ||
             (e = queue_count(S, QA, tmp + t_cub, cub_bytes, s))) {
@@ -1835,23 +1863,19 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
         }
     }
     if ((e = cudaGetLastError()) ||
-        (e = cudaMemcpyAsync(stage + o_sum, tmp + t_sum, (kNumClassPairs + 2) * sizeof(long long),
-                             cudaMemcpyDeviceToHost, s)) ||
-        (e = cudaMemcpyAsync(stage + o_ccost, tmp + t_ccost, kNumClassPairs * sizeof(double),
-                             cudaMemcpyDeviceToHost, s)) ||
-        (e = cudaMemcpyAsync(stage + o_nkept, A.npp_prefix + npair, sizeof(long long), cudaMemcpyDeviceToHost, s)) ||
-        (e = cudaMemcpyAsync(stage + o_bad, p->counters + nc2, sizeof(int), cudaMemcpyDeviceToHost, s)) ||
+        (e = cudaMemcpyAsync(stage + o_sum, tmp + t_sum, t_bad + sizeof(int) - t_sum, cudaMemcpyDeviceToHost, s)) ||
         (e = cudaStreamSynchronize(s))) {
         release_temp(); plan_free(p);
         return cuda_fail(ctx, e, "plan_create bound pass");
     }
-    if (*reinterpret_cast<const int *>(stage + o_bad)) {
+    const char *sum = stage + o_sum;
+    if (*reinterpret_cast<const int *>(sum + (t_bad - t_sum))) {
         release_temp(); plan_free(p);
         return fail(ctx, MOLINTS_ERR_INVALID, "plan_create: zero contracted function");
     }
-    const long long *qsum = reinterpret_cast<const long long *>(stage + o_sum);
-    const double *qcost = reinterpret_cast<const double *>(stage + o_ccost);
-    p->nprim_pair_kept = *reinterpret_cast<const long long *>(stage + o_nkept);
+    const long long *qsum = reinterpret_cast<const long long *>(sum);
+    const double *qcost = reinterpret_cast<const double *>(sum + (t_ccost - t_sum));
+    p->nprim_pair_kept = *reinterpret_cast<const long long *>(sum + (t_nkept - t_sum));
     const long long nq = qsum[kNumClassPairs];
     p->n_zero = qsum[kNumClassPairs + 1];
     if (nq > INT32_MAX) {
@@ -2006,7 +2030,7 @@ static int plan_enqueue(molints_plan *p, double *out_device, bool timing, JKOut 
     if (p->npair > 0) {
         if (int rc = mark(launches, "build_pairs", 0, s)) return rc;
         build_pairs_kernel<<<build_pairs_blocks(p->npair), 128, 0, s>>>(
-            p->npair, p->pair_ab, p->info, p->pp_src, p->sh_xyz, p->sh_poff, p->expn, p->ncoef,
+            p->npair, p->pair_ab, p->info, p->pp_src, nullptr, p->sh_xyz, p->sh_poff, p->expn, p->ncoef,
             std::sqrt(2.0) * std::pow(M_PI, 1.25), p->pbk, p->pp, p->geo, clear_in_build ? out_device : nullptr,
             clear_in_build ? (long long)p->npacked : 0);
         if (int rc = mark(launches, "build_pairs", 1, s)) return rc;
@@ -2026,7 +2050,9 @@ static int plan_enqueue(molints_plan *p, double *out_device, bool timing, JKOut 
     // Profiling runs every launch on the caller's stream, so each event pair times one kernel.
     const int ngen = p->n_gq > 0;
     const int nside = p->profiling ? 0
-                                   : std::min<int>(p->two_phase ? molints_ctx::kSideTwoPhase : molints_ctx::kSide,
+                                   : std::min<int>(p->two_phase ? molints_ctx::kSideTwoPhase
+                                                   : timing && jobs.size() <= 32 ? molints_ctx::kSideEager
+                                                                                 : molints_ctx::kSide,
                                                    (int)jobs.size() + ngen);
     int fp32_launches = 0;
     if (nside > 0) MI_CUDA(ctx, cudaEventRecord(ctx->fork, s));
@@ -2260,17 +2286,27 @@ static int plan_host_tables(const molints_plan *cp) {
     if (p->host_tables) return MOLINTS_OK;
     molints_ctx *ctx = p->ctx;
     const int n = p->npair;
-    std::vector<int2> ab(n);
-    std::vector<int4> info(n);
     p->bnd_h.resize(n);
     MI_CUDA(ctx, cudaSetDevice(ctx->device));
+    const char *ab0 = reinterpret_cast<const char *>(p->pair_ab), *host = nullptr;
+    const size_t o_info = reinterpret_cast<const char *>(p->info) - ab0, o_bnd = reinterpret_cast<const char *>(p->bnd) - ab0;
+    std::vector<char> own;
     if (n > 0) {
-        MI_CUDA(ctx, cudaMemcpyAsync(ab.data(), p->pair_ab, n * sizeof(int2), cudaMemcpyDeviceToHost, ctx->stream));
-        MI_CUDA(ctx, cudaMemcpyAsync(info.data(), p->info, n * sizeof(int4), cudaMemcpyDeviceToHost, ctx->stream));
-        MI_CUDA(ctx, cudaMemcpyAsync(p->bnd_h.data(), p->bnd, n * sizeof(double2), cudaMemcpyDeviceToHost,
-                                     ctx->stream));
+        // pair_ab, info and bnd lie together in the slab; the pinned upload buffer is free between
+        // plan creations, which are this thread's
+        const size_t bytes = o_bnd + n * sizeof(double2);
+        char *to = ctx->stage;
+        if (ctx->stage_bytes < bytes) {
+            own.resize(bytes);
+            to = own.data();
+        }
+        MI_CUDA(ctx, cudaMemcpyAsync(to, ab0, bytes, cudaMemcpyDeviceToHost, ctx->stream));
         MI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        host = to;
+        std::memcpy(p->bnd_h.data(), host + o_bnd, n * sizeof(double2));
     }
+    const int2 *ab = reinterpret_cast<const int2 *>(host);
+    const int4 *info = reinterpret_cast<const int4 *>(host + o_info);
     std::vector<int> first(std::max(p->nmol, 1), 0);  // first global shell of each molecule
     for (int m = 1; m < p->nmol; ++m) first[m] = first[m - 1] + p->mol_nshell[m - 1];
     p->pair_ref.resize(n);
@@ -2417,8 +2453,8 @@ int molints_plan_schwarz(molints_plan *p, double *out) {
     for (int c = 0; c < kNumPairClasses; ++c) {
         const int n = p->class_start[c + 1] - p->class_start[c];
         if (n <= 0) continue;
-        if (kSchwarzLaunchers[c]) kSchwarzLaunchers[c](P, B, p->class_start[c], n, nullptr, p->qcon, 1, ctx->stream);
-        else kRysBoundLaunchers[c](P, ctx->rys, p->class_start[c], n, nullptr, p->qcon, 1, ctx->stream);
+        if (kSchwarzLaunchers[c]) kSchwarzLaunchers[c](P, B, p->class_start[c], n, nullptr, nullptr, nullptr, p->qcon, 1, ctx->stream);
+        else kRysBoundLaunchers[c](P, ctx->rys, p->class_start[c], n, nullptr, nullptr, nullptr, p->qcon, 1, ctx->stream);
     }
     MI_CUDA(ctx, cudaGetLastError());
     std::vector<double> q(p->npair);

@@ -2,6 +2,8 @@
 // tables and the work queues.
 #include "plan_build.cuh"
 
+#include <algorithm>
+
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
@@ -12,49 +14,41 @@ constexpr int kThreads = 256;
 
 inline unsigned blocks_for(long long n) { return (unsigned)((n + kThreads - 1) / kThreads); }
 
-__global__ void pair_src_kernel(int npair, const int2 *__restrict__ ab1, const int4 *__restrict__ info1,
-                                const int *__restrict__ sh_K, int *__restrict__ src1) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= npair) return;
-    const int4 in = info1[k];
-    const int kb = sh_K[ab1[k].y];
-    for (int x = 0, ia = 0, ib = 0; x < in.y; ++x) {
-        src1[in.x + x] = (ia << 8) | ib;
-        if (++ib == kb) { ib = 0; ++ia; }
-    }
+// Bits of a pair's key below its run: the kept count, descending, and (plans that screen quartets)
+// the Qabs bucket above it.
+__host__ __device__ inline int within_bits(int maxnpp, int screen_sort) {
+    return bits_of((unsigned long long)maxnpp) + (screen_sort ? 8 : 0);
 }
 
-// max over a molecule's pairs of Qabs = sum_k b_k (every primitive pair), summed in list order
-// as the screening needs it.  The sums are >= 0, so their bit patterns order like the values.
-__global__ void pair_qmax_kernel(PlanBuildArgs A) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= A.npair) return;
-    const int4 in = A.info1[k];
-    double q = 0.0;
-    for (int x = 0; x < in.y; ++x) q += A.pbound[in.x + x].x;
-    atomicMax(&A.qmax[A.rec1[k].x], (unsigned long long)__double_as_longlong(q));
-}
-
-// Per stage-1 pair: primitive pairs kept (b_k * max Qabs of the molecule >= prim_cutoff; each
-// dropped term of any integral is below prim_cutoff by the Schwarz inequality), the pair's
-// bounds Qabs = sum of kept b_k and R = (1 + |AB|)^lb sum of kept w_k, and its sort key:
-// (class, molecule[, ms]) run first, then kept count descending (plans that screen quartets:
-// Qabs bucket descending, then kept count descending).
+// Per stage-1 pair, a warp each, its lanes over the primitive pairs: those kept (b_k * max Qabs of
+// the molecule >= prim_cutoff; each dropped term of any integral is below prim_cutoff by the Schwarz
+// inequality), the pair's bounds Qabs = sum of kept b_k and R = (1 + |AB|)^lb sum of kept w_k, and
+// its sort key: (class, molecule[, ms]) run first, then kept count descending (plans that screen
+// quartets: Qabs bucket descending, then kept count descending).  The sums run in list order, so that
+// the kept sum never exceeds the bound pass's sum over all primitive pairs.
 __global__ void pair_screen_kernel(PlanBuildArgs A) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (k >= A.npair) return;
     const int4 in = A.info1[k];
     const int4 r = A.rec1[k];
     const double qm = __longlong_as_double((long long)A.qmax[r.x]);
     double qa = 0.0, wa = 0.0;
     int kept = 0;
-    for (int x = 0; x < in.y; ++x) {
-        const double2 b = A.pbound[in.x + x];
-        if (A.prim_cutoff > 0.0 && b.x * qm < A.prim_cutoff) continue;
-        ++kept;
-        qa += b.x;
-        wa += b.y;
+    for (int x0 = 0; x0 < in.y; x0 += 32) {
+        const int n = min(32, in.y - x0);
+        double2 b = make_double2(0.0, 0.0);
+        if (lane < n) b = A.pbound[in.x + x0 + lane];
+        const unsigned keep = __ballot_sync(0xffffffffu, lane < n && !(A.prim_cutoff > 0.0 && b.x * qm < A.prim_cutoff));
+        kept += __popc(keep);
+        for (int x = 0; x < n; ++x) {
+            const double bx = __shfl_sync(0xffffffffu, b.x, x), by = __shfl_sync(0xffffffffu, b.y, x);
+            if ((keep >> x) & 1) {
+                qa += bx;
+                wa += by;
+            }
+        }
     }
+    if (lane) return;
     const int2 ab = A.ab1[k];
     const double dx = A.xyz[3 * ab.x] - A.xyz[3 * ab.y], dy = A.xyz[3 * ab.x + 1] - A.xyz[3 * ab.y + 1],
                  dz = A.xyz[3 * ab.x + 2] - A.xyz[3 * ab.y + 2];
@@ -64,10 +58,9 @@ __global__ void pair_screen_kernel(PlanBuildArgs A) {
     A.npp1[k] = kept;
     if (kept == 0) atomicAdd(A.n_zero, 1ull);
     A.bnd1[k] = make_double2(qa, wa * f);
-    const unsigned long long within =
-        A.screen_sort ? ((unsigned long long)(255 - qabs_bucket(qa)) << 12) | (unsigned long long)(0xFFF - min(kept, 0xFFF))
-                      : (unsigned long long)(0xFFFFF - kept);
-    A.key1[k] = ((unsigned long long)A.seg1[k] << 20) | within;
+    unsigned long long within = (unsigned long long)(A.maxnpp - kept);
+    if (A.screen_sort) within |= (unsigned long long)(255 - qabs_bucket(qa)) << bits_of((unsigned long long)A.maxnpp);
+    A.key1[k] = ((unsigned long long)A.seg1[k] << within_bits(A.maxnpp, A.screen_sort)) | within;
     A.idx1[k] = k;
 }
 
@@ -77,25 +70,34 @@ __global__ void pair_npp_kernel(PlanBuildArgs A) {
     A.npp[k] = k < A.npair ? A.npp1[A.idx2[k]] : 0;
 }
 
-// Final pair k (the stage-1 pair idx2[k]): its tables, with the kept primitive pairs packed
-// at npp_prefix[k], in stage-1 order.
+// Final pair k (the stage-1 pair idx2[k]), a warp each: its tables, with the kept primitive pairs
+// packed at npp_prefix[k], in stage-1 order.
 __global__ void pair_tables_kernel(PlanBuildArgs A) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (k >= A.npair) return;
     const int k1 = A.idx2[k];
     const int4 in = A.info1[k1];
     const int4 r = A.rec1[k1];
+    const int2 ab = A.ab1[k1];
+    const int kb = A.sh_K[ab.y];
     const int off = (int)A.npp_prefix[k];
     const double qm = __longlong_as_double((long long)A.qmax[r.x]);
     int j = off;
-    for (int x = 0; x < in.y; ++x) {
-        const double2 b = A.pbound[in.x + x];
-        if (A.prim_cutoff > 0.0 && b.x * qm < A.prim_cutoff) continue;
-        A.pp_src[j] = A.src1[in.x + x];
-        A.pbk[j] = b.x;
-        ++j;
+    for (int x0 = 0; x0 < in.y; x0 += 32) {
+        const int x = x0 + lane;
+        double2 b = make_double2(0.0, 0.0);
+        if (x < in.y) b = A.pbound[in.x + x];
+        const bool mine = x < in.y && !(A.prim_cutoff > 0.0 && b.x * qm < A.prim_cutoff);
+        const unsigned keep = __ballot_sync(0xffffffffu, mine);
+        if (mine) {
+            const int at = j + __popc(keep & ((1u << lane) - 1));
+            A.pp_src[at] = prim_src(x, kb);
+            A.pbk[at] = b.x;
+        }
+        j += __popc(keep);
     }
-    A.pair_ab[k] = A.ab1[k1];
+    if (lane) return;
+    A.pair_ab[k] = ab;
     A.info[k] = make_int4(off, j - off, in.z, in.w);
     A.bnd[k] = A.bnd1[k1];
     A.ms[k] = r.w;
@@ -198,7 +200,10 @@ __global__ void queue_summary_kernel(const QueueSetup S, QueueArgs A) {
     const int ci = blockIdx.x;
     if (threadIdx.x == 0) {
         A.summary[ci] = A.off[S.item_base[ci]];
-        if (ci == kNumClassPairs - 1) A.summary[kNumClassPairs] = A.off[A.n_items];
+        if (ci == kNumClassPairs - 1) {
+            A.summary[kNumClassPairs] = A.off[A.n_items];
+            *A.nkept = A.npp_prefix[A.npair];
+        }
     }
     __shared__ double part[kThreads];
     double s = 0.0;
@@ -250,27 +255,22 @@ __global__ void queue_place_kernel(QueueEmitArgs E) {
 
 }  // namespace
 
-cudaError_t plan_stage1_src(int npair, const int2 *ab1, const int4 *info1, const int *sh_K, int *src1,
-                            cudaStream_t s) {
-    if (npair <= 0) return cudaSuccess;
-    pair_src_kernel<<<blocks_for(npair), kThreads, 0, s>>>(npair, ab1, info1, sh_K, src1);
-    return cudaGetLastError();
-}
-
 size_t plan_build_temp_bytes(int npair) {
     size_t a = 0, b = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, a, (unsigned long long *)nullptr, (unsigned long long *)nullptr,
-                                    (int *)nullptr, (int *)nullptr, npair, 0, 52);
+                                    (int *)nullptr, (int *)nullptr, npair, 0, 64);
     cub::DeviceScan::ExclusiveSum(nullptr, b, (int *)nullptr, (long long *)nullptr, npair + 1);
     return a > b ? a : b;
 }
 
 cudaError_t plan_build_pairs(const PlanBuildArgs &A, void *temp, size_t temp_bytes, cudaStream_t s) {
     if (A.npair <= 0) return cudaSuccess;
-    pair_qmax_kernel<<<blocks_for(A.npair), kThreads, 0, s>>>(A);
-    pair_screen_kernel<<<blocks_for(A.npair), kThreads, 0, s>>>(A);
+    pair_screen_kernel<<<blocks_for(32LL * A.npair), kThreads, 0, s>>>(A);
     size_t tb = temp_bytes;
-    cudaError_t e = cub::DeviceRadixSort::SortPairs(temp, tb, A.key1, A.key2, A.idx1, A.idx2, A.npair, 0, 52, s);
+    // only the key's bits in use (a pass of the sort each 8)
+    const int bits = within_bits(A.maxnpp, A.screen_sort) + bits_of((unsigned long long)(A.npair - 1));
+    cudaError_t e = cub::DeviceRadixSort::SortPairs(temp, tb, A.key1, A.key2, A.idx1, A.idx2, A.npair, 0,
+                                                    std::max(1, bits), s);
     if (e != cudaSuccess) return e;
     pair_npp_kernel<<<blocks_for(A.npair + 1), kThreads, 0, s>>>(A);
     // kept primitive pairs before each final pair (their sum is below 2^31: stage-1 offsets
@@ -278,7 +278,7 @@ cudaError_t plan_build_pairs(const PlanBuildArgs &A, void *temp, size_t temp_byt
     tb = temp_bytes;
     e = cub::DeviceScan::ExclusiveSum(temp, tb, A.npp, A.npp_prefix, A.npair + 1, s);
     if (e != cudaSuccess) return e;
-    pair_tables_kernel<<<blocks_for(A.npair), kThreads, 0, s>>>(A);
+    pair_tables_kernel<<<blocks_for(32LL * A.npair), kThreads, 0, s>>>(A);
     return cudaGetLastError();
 }
 

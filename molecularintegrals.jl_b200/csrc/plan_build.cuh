@@ -146,22 +146,35 @@ struct QueueSetup {
     int zero_trunc;
 };
 
+// Primitive pair x of a pair whose second shell has kb primitives: (ia << 8) | ib, A's outer.
+__host__ __device__ inline int prim_src(int x, int kb) {
+    const int ia = x / kb;
+    return (ia << 8) | (x - ia * kb);
+}
+
+// Bits of values 0 .. v.
+__host__ __device__ inline int bits_of(unsigned long long v) {
+    int b = 0;
+    while (v >> b) ++b;
+    return b;
+}
+
 // Device arrays of one device plan build (all owned by the caller).
 struct PlanBuildArgs {
     int npair;
     int nall;                      // stage-1 primitive pairs
+    int maxnpp;                    // the most primitive pairs of a pair
     double prim_cutoff;
     int screen_sort;               // order runs by Qabs bucket (descending), then kept count
     // stage 1 (pair order by class, molecule[, ms], all-primitive count)
     const int2 *ab1;               // global shells (A, B)
     const int4 *info1;             // {first primitive pair, count, first function of A, of B}
-    const int *src1;               // primitive pair -> (ia << 8) | ib
     const int4 *rec1;              // {molecule, reference pair index, class | swapped << 8, ms}
     const int *seg1;               // first stage-1 pair of the pair's (class, molecule[, ms]) run
     const double2 *pbound;         // per primitive pair: (b_k, w_k) of the bound pass
     const double *xyz;             // shell centres
-    const int *sh_L;
-    unsigned long long *qmax;      // per molecule, zeroed: max over pairs of sum b_k (bits)
+    const int *sh_L, *sh_K;
+    const unsigned long long *qmax;  // per molecule: max over pairs of sum b_k (bits), from the bound pass
     unsigned long long *n_zero;    // zeroed: pairs without kept primitive pairs
     // re-sort scratch
     int *npp1;                     // kept count per stage-1 pair
@@ -180,11 +193,6 @@ struct PlanBuildArgs {
     int *g_pair;                   // two-phase: per molecule shell pair, or null
     const long long *g_mol;        // two-phase: per molecule {.., first pair entry, ..}
 };
-
-// Stage-1 primitive-pair list: pair k's K_A x K_B entries (ia << 8) | ib, A's primitive
-// outer, at info1[k].x.
-cudaError_t plan_stage1_src(int npair, const int2 *ab1, const int4 *info1, const int *sh_K, int *src1,
-                            cudaStream_t s);
 
 // Screening, re-sort and final pair tables.  temp: CUB scratch of at least
 // plan_build_temp_bytes(npair) bytes.
@@ -209,6 +217,8 @@ struct QueueArgs {
     long long *off;                // n_items + 1
     long long *summary;            // kNumClassPairs + 1
     double *class_cost;            // kNumClassPairs
+    long long *nkept;              // kept primitive pairs
+    int npair;
 };
 cudaError_t queue_count(const QueueSetup &S, const QueueArgs &A, void *temp, size_t temp_bytes,
                         cudaStream_t s);

@@ -430,11 +430,13 @@ __device__ __forceinline__ void rys_queue_body(const EriQueue &Q, const RysTab &
 
 // Bounds of the pairs [p0, p0+np) of a pair class (bra class == ket class), one group per pair:
 // full == 0: for every primitive pair k, from the diagonal primitive quartet,
-//   pbound[k] = {sqrt(max |(a_k b_k|a_k b_k)|), sqrt(max |[e0|e0]_kk|)};
+//   pbound[k] = {sqrt(max |(a_k b_k|a_k b_k)|), sqrt(max |[e0|e0]_kk|)},
+//   qmax[mol[p]]: the largest sum of the first over the molecule's pairs, as bits;
 // full != 0: the contracted Q_p = sqrt(max |(ab|ab)|) into qout[p].
 template <class C>
 __device__ __forceinline__ void rys_bound_body(const PairTab &P, const RysTab &R, const RysClassTabs &T,
-                                               int p0, int np, double2 *pbound, double *qout, int full) {
+                                               int p0, int np, double2 *pbound, const int *mol,
+                                               unsigned long long *qmax, double *qout, int full) {
     extern __shared__ __align__(16) double rys_smem[];
     __shared__ double s_red[4];
     constexpr int NG = 128 / C::G;
@@ -447,6 +449,7 @@ __device__ __forceinline__ void rys_bound_body(const PairTab &P, const RysTab &R
     const int4 in = __ldg(&P.info[p]);
     const double4 g = ldg4(&P.geo[p]);
     const int nk = full ? 1 : in.y;
+    double q = 0.0;  // sum of b_k in list order
     for (int k = 0; k < nk; ++k) {
         const int i0 = full ? 0 : k, n = full ? in.y : 1;
         const RysKets K{in.x + i0, L.w1 == 0 ? n * n : 0, L.w2 == 0 ? n * n : 0, n * n, false, false};
@@ -464,8 +467,11 @@ __device__ __forceinline__ void rys_bound_body(const PairTab &P, const RysTab &R
             if (full) qout[p] = sqrt(m);
             else pbound[in.x + k] = make_double2(sqrt(m), sqrt(wmax));
         }
+        q += sqrt(m);
         group_sync<C::G>(gid);
     }
+    // the sums are >= 0, so their bit patterns order like the values
+    if (!full && lane == 0) atomicMax(&qmax[__ldg(&mol[p])], (unsigned long long)__double_as_longlong(q));
 }
 
 }  // namespace molints
