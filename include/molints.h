@@ -253,10 +253,11 @@ int molints_plan_jk(molints_plan *plan, const double *D_device, double *J_device
 /* The same from host arrays in one synchronous call (plan, device buffers, copies). */
 int molints_jk(molints_ctx *ctx, const molints_basis *basis, const molints_options *opts,
                const double *D_host, double *J_host, double *K_host);
-/* enable != 0: the next execute captures the plan's whole device path (pair build, counter
- * reset, every class-pair kernel on the forked side streams) into a CUDA graph on the
- * context's stream, and later executes into the same out_device launch that graph (a new
- * out_device recaptures).  Not combined with profiling.  No reference counterpart. */
+/* enable != 0: the second execute in a row into the same out_device captures the plan's whole
+ * device path (pair build, counter reset, every class-pair kernel on the forked side streams) into
+ * a CUDA graph on the context's stream, and later executes into that out_device launch the graph
+ * (another out_device starts over; an execute that is not followed by a second one into its output
+ * pays for no capture).  Not combined with profiling.  No reference counterpart. */
 int molints_plan_set_graph(molints_plan *plan, int enable);
 int molints_plan_stats(const molints_plan *plan, molints_stats *stats);
 /* Per class pair x >= y (entry x * MOLINTS_NUM_PAIR_CLASSES + y, n = MOLINTS_NUM_PAIR_CLASSES^2):

@@ -61,11 +61,13 @@ struct molints_ctx {
     // two-phase plans, whose kernels fill the device and share L2 with the scratch they write, take
     // kSideTwoPhase.  On B200, us per execute with 6 / 16 / 24 streams: 8 polarised atoms 99 / 87 /
     // 78, 11 atoms with f shells 340 / 277 / 254, 15 polarised atoms 324 / 329 / 335, a batch of
-    // 1.17e9 integrals 7025 / 7139 / 7253.
+    // 1.17e9 integrals 7025 / 7139 / 7253; capturing and instantiating a graph of 13 polarised atoms
+    // takes 0.65 / 1.2 / 1.6 ms.
     // Executes that are not captured take kSideEager unless they launch many kernels (f shells): each
     // stream costs three calls of the host (8 polarised atoms, 22 launches, us of host and total
     // with 24 / 8 streams: 118, 128 / 112, 127; 11 atoms with f shells, 57 launches: 296, 308 / 265, 373).
-    static constexpr int kSide = 24, kSideEager = 8, kSideTwoPhase = 6;
+    static constexpr int kSide = 16, kSideEager = 8, kSideTwoPhase = 6;
+    static_assert(kSide >= kNumPairClasses - 1 && kSide > kSideTwoPhase, "the bound pass and the zero rows use side streams too");
     cudaStream_t side[kSide] = {};
     cudaEvent_t fork = nullptr, join[kSide] = {};
     int num_sms = 0;
@@ -163,6 +165,7 @@ struct molints_plan {
     int use_graph = 0;
     cudaGraphExec_t gexec = nullptr;
     double *graph_out = nullptr;
+    double *graph_seen = nullptr;      // the last uncaptured execute's output
     int graph_gen = -1;                // the context's scratch_gen at capture
     // per-launch profiling (molints_plan_set_profiling)
     int profiling = 0;
@@ -2178,9 +2181,15 @@ int molints_plan_execute(molints_plan *p, double *out_device) {
 static int plan_execute_impl(molints_plan *p, double *out_device) {
     molints_ctx *ctx = p->ctx;
     if (!p->use_graph || p->profiling) return plan_enqueue(p, out_device, true);
-    // CUDA graph: captured once per output pointer (and scratch buffer), then launched whole
+    // CUDA graph: captured at the second execute in a row into an output (and scratch buffer), then
+    // launched whole.  The first runs uncaptured: capture and instantiation cost more than they save
+    // one execute (13 polarised atoms on B200: 1.6 ms against 0.21 ms for the execute).
     cudaStream_t s = ctx->stream;
     if (!p->gexec || p->graph_out != out_device || (p->two_phase && p->graph_gen != ctx->scratch_gen)) {
+        if (p->graph_seen != out_device) {
+            p->graph_seen = out_device;
+            return plan_enqueue(p, out_device, true);
+        }
         if (p->gexec) {
             cudaGraphExecDestroy(p->gexec);
             p->gexec = nullptr;
@@ -2271,6 +2280,7 @@ int molints_jk(molints_ctx *ctx, const molints_basis *b, const molints_options *
 int molints_plan_set_graph(molints_plan *p, int enable) {
     if (!p) return MOLINTS_ERR_INVALID;
     p->use_graph = enable ? 1 : 0;
+    p->graph_seen = nullptr;
     if (!enable && p->gexec) {
         cudaSetDevice(p->ctx->device);
         cudaGraphExecDestroy(p->gexec);

@@ -252,7 +252,7 @@ class Plan:
                                                            ctypes.c_void_p(J_ptr), ctypes.c_void_p(K_ptr)))
 
     def set_graph(self, enable: bool = True) -> None:
-        """Launch executes as one captured CUDA graph (recaptured for a new output pointer)."""
+        """Launch executes as one captured CUDA graph (from the second one in a row into an output)."""
         self.engine._check(self.engine.lib.molints_plan_set_graph(self.h, int(enable)))
 
     def set_profiling(self, enable: bool = True) -> None:
