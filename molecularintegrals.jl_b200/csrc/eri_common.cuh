@@ -8,7 +8,7 @@
 //       geo[p]  = {A-B (x,y,z), unused}                    (double4, 32 B)
 //       bnd[p]  = {Qabs_p, R_p}: bounds for screening and for FP32 quartets (double2)
 //   * primitive pairs, 80 B each (5 x 16 B vector loads): PrimPair below;
-//   * the Boys table (T = 0..40 step 1/16, F_0..F_22 and e^-T per row);
+//   * the Boys tables (T = 0..40 step 1/32), 32 bytes per order and point;
 //   * the packed output vector, 0-based iindex order (src/Utils.jl:14-19).
 #pragma once
 #include <cuda_runtime.h>
@@ -16,14 +16,14 @@
 
 namespace molints {
 
-constexpr int kBoysRows = 641;            // T_n = n/16, n = 0..640 (T up to 40)
-constexpr int kBoysCols = 24;             // F_0..F_22 at T_n, then e^-T_n
-constexpr int kBoysTaylor = 8;            // Taylor terms about T_n; |T - T_n| <= 1/32
-constexpr double kBoysStepInv = 16.0;
-constexpr double kBoysStep = 0.0625;
+constexpr int kBoysRows = 1281;           // T_n = n/32, n = 0..1280 (T up to 40)
+constexpr int kBoysTaylor = 7;            // Taylor terms about T_n; |T - T_n| <= 1/64
+constexpr double kBoysStepInv = 32.0;
+constexpr double kBoysStep = 0.03125;
 constexpr double kBoysTableMax = 40.0;    // exact-mode switch to the asymptotic form
-constexpr int kBoysMaxM1 = 16;            // scaled tables exist for M = 0..15
-constexpr int kBoysScaledCols = 10;       // F_{M+k}(T_n)/k! for k < 8, e^-T_n, pad (80 B)
+constexpr int kBoysMaxM1 = 16;            // tables exist for M = 0..15
+// Two tables of 16-byte rows per M: {F_M(T_n), e^-T_n} and {F_{M+6}(T_n)/6!, F_{M+3}(T_n)/3!}
+constexpr int kBoysHalf = 2 * kBoysRows;  // doubles of one of them
 constexpr double kBoysReferenceSwitch = 30.0;  // farray's Tmax, src/Boys.jl:19
 
 // Record of one primitive pair (a, b) of a canonical shell pair (A, B):
@@ -38,7 +38,7 @@ constexpr double kBoysReferenceSwitch = 30.0;  // farray's Tmax, src/Boys.jl:19
 // so that kab_bra * kab_ket / sqrt(zeta+eta) is the [00|00] prefactor of HGP eq. 12,
 // 2 pi^(5/2) / (zeta eta sqrt(zeta+eta)) x exp(...) x coefficients.
 struct PrimPair {
-    double zeta, kab, oo2z, px, py, pz, pax, pay, paz, b;
+    double zeta, kab, px, py, pz, oo2z, pax, pay, paz, b;  // what (ss| needs comes first
 };
 static_assert(sizeof(PrimPair) == 80, "PrimPair is 5 x 16 bytes");
 
@@ -50,8 +50,7 @@ struct PairTab {
 };
 
 struct BoysTab {
-    const double *tab;     // [kBoysRows][kBoysCols]: F_0..F_22, e^-T_n
-    const double *scaled;  // [kBoysMaxM1][kBoysRows][kBoysScaledCols]
+    const double *tab;     // [kBoysMaxM1][2][kBoysRows][2] (fill_boys_table)
     double t_switch;       // asymptotic form at T >= t_switch
 };
 
@@ -108,50 +107,55 @@ __device__ __forceinline__ PrimPair load_pp(const PrimPair *__restrict__ base, i
     const double2 a = __ldg(v), b = __ldg(v + 1), c = __ldg(v + 2), d = __ldg(v + 3),
                   e = __ldg(v + 4);
     PrimPair r;
-    r.zeta = a.x; r.kab = a.y; r.oo2z = b.x; r.px = b.y; r.py = c.x; r.pz = c.y;
+    r.zeta = a.x; r.kab = a.y; r.px = b.x; r.py = b.y; r.pz = c.x; r.oo2z = c.y;
     r.pax = d.x; r.pay = d.y; r.paz = e.x; r.b = e.y;
     return r;
 }
 
 // F_0..F_M at T: the farray structure of src/Boys.jl:19-27.
-//   T <  t_switch: F_M by an 8-term Taylor expansion about the nearest table point,
-//                  F_M(T_n - d) = sum_k [F_{M+k}(T_n)/k!] d^k (the table row of M holds the
-//                  bracketed coefficients, so this is 7 FMAs), e^-T = e^-T_n e^d, then the
-//                  downward recursion F_m = (2T F_{m+1} + e^-T) / (2m+1).
+//   T <  t_switch: F_M by a 7-term Taylor expansion about the nearest table point,
+//                  F_M(T_n - d) = sum_k c_k d^k, c_k = F_{M+k}(T_n)/k!, then e^-T = e^-T_n e^d and
+//                  the downward recursion F_m = (2T F_{m+1} + e^-T) / (2m+1).  Of the c_k only c_0,
+//                  c_3 and c_6 are read; the others follow by the same recursion at T_n (all terms
+//                  positive, and what rounding it adds comes times d <= 1/64).  A warp's lanes read
+//                  rows at random, so every 16 bytes of a row cost about eight passes of the L1
+//                  data pipe, which was what bound the (ss|ss) and (ps|ss) kernels (78-83 % busy
+//                  with all of c_0 .. c_7 read, in 80-byte rows; the FP64 pipe 40-54 %): BOYSFIG.
 //   T >= t_switch: the asymptotic family F_m = (2m-1)!! / (2T)^m * sqrt(pi/T)/2, the values
 //                  farray's Fm_asymp top order and e^-T-free recursion produce.
-// The table index is rounded with the 1.5*2^52 trick: T*16 + 1.5*2^52 holds round(T*16) in
-// its low mantissa bits, and subtracting the constant back gives T_n*16 exactly.
+// The table index is rounded with the 1.5*2^52 trick: T*32 + 1.5*2^52 holds round(T*32) in
+// its low mantissa bits, and subtracting the constant back gives T_n*32 exactly.
 template <int M>
 __device__ __forceinline__ void boys_fm(double T, const BoysTab &bt, double *F) {
     static_assert(M < kBoysMaxM1, "Boys order beyond the scaled tables");
     if (T < bt.t_switch) {
         constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52
-        const double t16 = fma(T, kBoysStepInv, kMagic);
-        const int n = __double2loint(t16);
-        const double d = fma(t16 - kMagic, kBoysStep, -T);
-        const double2 *__restrict__ r2 = reinterpret_cast<const double2 *>(
-            bt.scaled + ((size_t)M * kBoysRows + n) * kBoysScaledCols);
-        const double2 c01 = __ldg(r2), c23 = __ldg(r2 + 1), c45 = __ldg(r2 + 2), c67 = __ldg(r2 + 3);
-        double f = fma(c67.y, d, c67.x);
-        f = fma(f, d, c45.y);
-        f = fma(f, d, c45.x);
-        f = fma(f, d, c23.y);
-        f = fma(f, d, c23.x);
-        f = fma(f, d, c01.y);
-        f = fma(f, d, c01.x);
+        const double t32 = fma(T, kBoysStepInv, kMagic);
+        const int n = __double2loint(t32);
+        const double tn = (t32 - kMagic) * kBoysStep, d = tn - T;
+        const double2 *__restrict__ tab = reinterpret_cast<const double2 *>(bt.tab + (size_t)M * (2 * kBoysHalf)) + n;
+        const double2 fe = __ldg(tab), c63 = __ldg(tab + kBoysRows);
+        // c_k = T_n c_{k+1} 2(k+1)/(2(M+k)+1) + e^-T_n / (k! (2(M+k)+1))
+        const double c5 = fma(tn * c63.x, 12.0 / (2 * M + 11), fe.y * (1.0 / (120.0 * (2 * M + 11))));
+        const double c2 = fma(tn * c63.y, 6.0 / (2 * M + 5), fe.y * (1.0 / (2.0 * (2 * M + 5))));
+        const double c4 = fma(tn * c5, 10.0 / (2 * M + 9), fe.y * (1.0 / (24.0 * (2 * M + 9))));
+        const double c1 = fma(tn * c2, 4.0 / (2 * M + 3), fe.y * (1.0 / (2 * M + 3)));
+        double f = fma(c63.x, d, c5);
+        f = fma(f, d, c4);
+        f = fma(f, d, c63.y);
+        f = fma(f, d, c2);
+        f = fma(f, d, c1);
+        f = fma(f, d, fe.x);
         F[M] = f;
         if (M > 0) {
-            const double emtn = __ldg(r2 + 4).x;
-            // e^d for |d| <= 1/32 by its Taylor polynomial to d^7
-            double ed = fma(d, 1.0 / 5040, 1.0 / 720);
-            ed = fma(ed, d, 1.0 / 120);
+            // e^d for |d| <= 1/64 by its Taylor polynomial to d^6
+            double ed = fma(d, 1.0 / 720, 1.0 / 120);
             ed = fma(ed, d, 1.0 / 24);
             ed = fma(ed, d, 1.0 / 6);
             ed = fma(ed, d, 0.5);
             ed = fma(ed, d, 1.0);
             ed = fma(ed, d, 1.0);
-            const double emt = emtn * ed;
+            const double emt = fe.y * ed;
             const double t2 = 2.0 * T;
 #pragma unroll
             for (int m = M - 1; m >= 0; --m) F[m] = fma(t2, F[m + 1], emt) * (1.0 / (2 * m + 1));

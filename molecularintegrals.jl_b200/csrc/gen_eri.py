@@ -217,6 +217,34 @@ def vrr_line(a, c, m):
     return f"const VT {vname(a, c, m)} = {s};"
 
 
+def vrr_terms(a, c):
+    """The recurrence of entry (a, c)^(0) as (factor, entry) products."""
+    if c == 0:
+        if a == 0:
+            return [("pref", "F[0]")]
+        i = shift_dir(a)
+        am = shift_minus(a, i)
+        amm = shift_minus(am, i)
+        x = XYZ[i]
+        t = [(f"PA{x}", vname(am, 0, 0)), (f"WP{x}", vname(am, 0, 1))]
+        if amm >= 0:
+            k = AO[am][i]
+            t.append((f"{k}.0 * oo2z", f"({vname(amm, 0, 0)} - rho_z * {vname(amm, 0, 1)})"))
+        return t
+    i = shift_dir(c)
+    cm = shift_minus(c, i)
+    cmm = shift_minus(cm, i)
+    am = shift_minus(a, i)
+    x = XYZ[i]
+    t = [(f"QC{x}", vname(a, cm, 0)), (f"WQ{x}", vname(a, cm, 1))]
+    if am >= 0:
+        t.append((f"{AO[a][i]}.0 * oo2ze", vname(am, cm, 1)))
+    if cmm >= 0:
+        k = AO[cm][i]
+        t.append((f"{k}.0 * oo2e", f"({vname(a, cmm, 0)} - rho_e * {vname(a, cmm, 1)})"))
+    return t
+
+
 # ------------------------------------------------------------------ HRR plan
 class HrrPlan:
     """(ab|cd) from the contracted [a0|c0] block: bra HRR then ket HRR (src/HGP.jl:92-114)."""
@@ -312,10 +340,35 @@ def emit_class_pair(X, Y, rys=False):
     na, nb, nc, nd = [len(shell_range(l)) for l in (la, lb, lc, ld)]
     nout = na * nb * nc * nd
     ind = "        "
-    vrr_code = "\n".join(ind + "    " + vrr_line(*k) for k in entries)
-    acc_code = "\n".join(
-        f"{ind}    acc[{hp.acc_index[(a, c)]}] += (double){vname(a, c, 0)};"
-        for a in hp.acc_a for c in hp.acc_c)
+    # entries that only go into the block: in FP64 their products are added to it one by one (an FMA
+    # each), without forming the entry; entries of the FP32 variant are formed and added in FP64
+    used = {d for k in entries for d in vrr_deps(*k)}
+    block = [(a, c) for a in hp.acc_a for c in hp.acc_c]
+    leaf = {(a, c) for a, c in block if (a, c, 0) not in used}
+    vrr_code = "\n".join(ind + "    " + vrr_line(*k) for k in entries if k[2] or (k[0], k[1]) not in leaf)
+    acc64, acc32 = [], []
+    for a, c in block:
+        i = hp.acc_index[(a, c)]
+        if (a, c) not in leaf:
+            acc64.append(f"acc[{i}] += (double){vname(a, c, 0)};")
+            acc32.append(acc64[-1])
+            continue
+        t = vrr_terms(a, c)
+        if M == 1 and a:  # (ps|ss): W - P = -rho_z (P - Q), used once an axis
+            x = XYZ[shift_dir(a)]
+            t = [(f"PA{x}", vname(0, 0, 0)), (f"PQ{x}", f"(-ez * {vname(0, 0, 1)})")]
+        e = f"acc[{i}]"
+        for f, v in t[::-1]:
+            e = f"fma({f}, {v}, {e})"
+        acc64.append(f"acc[{i}] = {e};")
+        acc32 += [vrr_line(a, c, 0), f"acc[{i}] += (double){vname(a, c, 0)};"]
+    has32 = len(entries) >= MIXED_MIN_VRR and not rys
+
+    def lines(x, extra=""):
+        return "\n".join(f"{ind}    {extra}{ln}" for ln in x)
+    acc_code = lines(acc64) if not has32 else (
+        f"{ind}    if constexpr (sizeof(VT) == 8) {{\n{lines(acc64, '    ')}\n{ind}    }} else {{\n"
+        f"{lines(acc32, '    ')}\n{ind}    }}")
     hrr_code = "\n".join("    " + ln for ln in hp.lines)
     out_code = []
     for x, (a, b, c, d, expr) in enumerate(hp.targets):
@@ -407,7 +460,6 @@ void launch_schwarz_{tag}(const PairTab &P, const BoysTab &B, int p0, int np, do
     schwarz_kernel_{tag}<<<(np + 3) / 4, 128, 0, s>>>(P, B, p0, np, pbound, mol, qmax, qout, full);
 }}
 """
-    has32 = len(entries) >= MIXED_MIN_VRR and not rys
     if nout <= STAGE_MAX_OUT:
         sbytes = 4 * 32 * nout * 8
         mixed_attr = (f"        cudaFuncSetAttribute(eri_queue_{tag}<1, 0>, "
@@ -525,13 +577,13 @@ __device__ __forceinline__ void vrr_{tag}(const PairTab &P, const BoysTab &B, in
             const double r = rsqrt(bra.zeta + ket.zeta);
             const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
-            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[{M + 1}];
             boys_fm<{M}>(T, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
-            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
             const VT WQx = (VT)(zz * PQx), WQy = (VT)(zz * PQy), WQz = (VT)(zz * PQz);
             const VT oo2z = (VT)bra.oo2z, oo2e = (VT)ket.oo2z, oo2ze = (VT)(0.5 * r2);

@@ -25,13 +25,13 @@ __device__ __forceinline__ void vrr_dddp(const PairTab &P, const BoysTab &B, int
             const double r = rsqrt(bra.zeta + ket.zeta);
             const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
-            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[8];
             boys_fm<7>(T, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
-            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
             const VT WQx = (VT)(zz * PQx), WQy = (VT)(zz * PQy), WQz = (VT)(zz * PQz);
             const VT oo2z = (VT)bra.oo2z, oo2e = (VT)ket.oo2z, oo2ze = (VT)(0.5 * r2);
@@ -904,812 +904,1311 @@ __device__ __forceinline__ void vrr_dddp(const PairTab &P, const BoysTab &B, int
             const VT v33_9_1 = QCz * v33_3_1 + WQz * v33_3_2 + (VT)3.0 * oo2ze * v18_3_2 + (VT)1.0 * oo2e * (v33_0_1 - rho_e * v33_0_2);
             const VT v34_9_0 = QCz * v34_3_0 + WQz * v34_3_1 + (VT)4.0 * oo2ze * v19_3_1 + (VT)1.0 * oo2e * (v34_0_0 - rho_e * v34_0_1);
             const VT v34_9_1 = QCz * v34_3_1 + WQz * v34_3_2 + (VT)4.0 * oo2ze * v19_3_2 + (VT)1.0 * oo2e * (v34_0_1 - rho_e * v34_0_2);
-            const VT v4_10_0 = QCx * v4_4_0 + WQx * v4_4_1 + (VT)2.0 * oo2ze * v1_4_1 + (VT)2.0 * oo2e * (v4_1_0 - rho_e * v4_1_1);
-            const VT v5_10_0 = QCx * v5_4_0 + WQx * v5_4_1 + (VT)1.0 * oo2ze * v2_4_1 + (VT)2.0 * oo2e * (v5_1_0 - rho_e * v5_1_1);
-            const VT v6_10_0 = QCx * v6_4_0 + WQx * v6_4_1 + (VT)1.0 * oo2ze * v3_4_1 + (VT)2.0 * oo2e * (v6_1_0 - rho_e * v6_1_1);
-            const VT v7_10_0 = QCx * v7_4_0 + WQx * v7_4_1 + (VT)2.0 * oo2e * (v7_1_0 - rho_e * v7_1_1);
-            const VT v8_10_0 = QCx * v8_4_0 + WQx * v8_4_1 + (VT)2.0 * oo2e * (v8_1_0 - rho_e * v8_1_1);
-            const VT v9_10_0 = QCx * v9_4_0 + WQx * v9_4_1 + (VT)2.0 * oo2e * (v9_1_0 - rho_e * v9_1_1);
-            const VT v10_10_0 = QCx * v10_4_0 + WQx * v10_4_1 + (VT)3.0 * oo2ze * v4_4_1 + (VT)2.0 * oo2e * (v10_1_0 - rho_e * v10_1_1);
-            const VT v11_10_0 = QCx * v11_4_0 + WQx * v11_4_1 + (VT)2.0 * oo2ze * v5_4_1 + (VT)2.0 * oo2e * (v11_1_0 - rho_e * v11_1_1);
-            const VT v12_10_0 = QCx * v12_4_0 + WQx * v12_4_1 + (VT)2.0 * oo2ze * v6_4_1 + (VT)2.0 * oo2e * (v12_1_0 - rho_e * v12_1_1);
-            const VT v13_10_0 = QCx * v13_4_0 + WQx * v13_4_1 + (VT)1.0 * oo2ze * v7_4_1 + (VT)2.0 * oo2e * (v13_1_0 - rho_e * v13_1_1);
-            const VT v14_10_0 = QCx * v14_4_0 + WQx * v14_4_1 + (VT)1.0 * oo2ze * v9_4_1 + (VT)2.0 * oo2e * (v14_1_0 - rho_e * v14_1_1);
-            const VT v15_10_0 = QCx * v15_4_0 + WQx * v15_4_1 + (VT)1.0 * oo2ze * v8_4_1 + (VT)2.0 * oo2e * (v15_1_0 - rho_e * v15_1_1);
-            const VT v16_10_0 = QCx * v16_4_0 + WQx * v16_4_1 + (VT)2.0 * oo2e * (v16_1_0 - rho_e * v16_1_1);
-            const VT v17_10_0 = QCx * v17_4_0 + WQx * v17_4_1 + (VT)2.0 * oo2e * (v17_1_0 - rho_e * v17_1_1);
-            const VT v18_10_0 = QCx * v18_4_0 + WQx * v18_4_1 + (VT)2.0 * oo2e * (v18_1_0 - rho_e * v18_1_1);
-            const VT v19_10_0 = QCx * v19_4_0 + WQx * v19_4_1 + (VT)2.0 * oo2e * (v19_1_0 - rho_e * v19_1_1);
-            const VT v20_10_0 = QCx * v20_4_0 + WQx * v20_4_1 + (VT)4.0 * oo2ze * v10_4_1 + (VT)2.0 * oo2e * (v20_1_0 - rho_e * v20_1_1);
-            const VT v21_10_0 = QCx * v21_4_0 + WQx * v21_4_1 + (VT)3.0 * oo2ze * v11_4_1 + (VT)2.0 * oo2e * (v21_1_0 - rho_e * v21_1_1);
-            const VT v22_10_0 = QCx * v22_4_0 + WQx * v22_4_1 + (VT)3.0 * oo2ze * v12_4_1 + (VT)2.0 * oo2e * (v22_1_0 - rho_e * v22_1_1);
-            const VT v23_10_0 = QCx * v23_4_0 + WQx * v23_4_1 + (VT)2.0 * oo2ze * v13_4_1 + (VT)2.0 * oo2e * (v23_1_0 - rho_e * v23_1_1);
-            const VT v24_10_0 = QCx * v24_4_0 + WQx * v24_4_1 + (VT)2.0 * oo2ze * v15_4_1 + (VT)2.0 * oo2e * (v24_1_0 - rho_e * v24_1_1);
-            const VT v25_10_0 = QCx * v25_4_0 + WQx * v25_4_1 + (VT)2.0 * oo2ze * v14_4_1 + (VT)2.0 * oo2e * (v25_1_0 - rho_e * v25_1_1);
-            const VT v26_10_0 = QCx * v26_4_0 + WQx * v26_4_1 + (VT)1.0 * oo2ze * v16_4_1 + (VT)2.0 * oo2e * (v26_1_0 - rho_e * v26_1_1);
-            const VT v27_10_0 = QCx * v27_4_0 + WQx * v27_4_1 + (VT)1.0 * oo2ze * v17_4_1 + (VT)2.0 * oo2e * (v27_1_0 - rho_e * v27_1_1);
-            const VT v28_10_0 = QCx * v28_4_0 + WQx * v28_4_1 + (VT)1.0 * oo2ze * v18_4_1 + (VT)2.0 * oo2e * (v28_1_0 - rho_e * v28_1_1);
-            const VT v29_10_0 = QCx * v29_4_0 + WQx * v29_4_1 + (VT)1.0 * oo2ze * v19_4_1 + (VT)2.0 * oo2e * (v29_1_0 - rho_e * v29_1_1);
-            const VT v30_10_0 = QCx * v30_4_0 + WQx * v30_4_1 + (VT)2.0 * oo2e * (v30_1_0 - rho_e * v30_1_1);
-            const VT v31_10_0 = QCx * v31_4_0 + WQx * v31_4_1 + (VT)2.0 * oo2e * (v31_1_0 - rho_e * v31_1_1);
-            const VT v32_10_0 = QCx * v32_4_0 + WQx * v32_4_1 + (VT)2.0 * oo2e * (v32_1_0 - rho_e * v32_1_1);
-            const VT v33_10_0 = QCx * v33_4_0 + WQx * v33_4_1 + (VT)2.0 * oo2e * (v33_1_0 - rho_e * v33_1_1);
-            const VT v34_10_0 = QCx * v34_4_0 + WQx * v34_4_1 + (VT)2.0 * oo2e * (v34_1_0 - rho_e * v34_1_1);
-            const VT v4_11_0 = QCx * v4_5_0 + WQx * v4_5_1 + (VT)2.0 * oo2ze * v1_5_1 + (VT)1.0 * oo2e * (v4_2_0 - rho_e * v4_2_1);
-            const VT v5_11_0 = QCx * v5_5_0 + WQx * v5_5_1 + (VT)1.0 * oo2ze * v2_5_1 + (VT)1.0 * oo2e * (v5_2_0 - rho_e * v5_2_1);
-            const VT v6_11_0 = QCx * v6_5_0 + WQx * v6_5_1 + (VT)1.0 * oo2ze * v3_5_1 + (VT)1.0 * oo2e * (v6_2_0 - rho_e * v6_2_1);
-            const VT v7_11_0 = QCx * v7_5_0 + WQx * v7_5_1 + (VT)1.0 * oo2e * (v7_2_0 - rho_e * v7_2_1);
-            const VT v8_11_0 = QCx * v8_5_0 + WQx * v8_5_1 + (VT)1.0 * oo2e * (v8_2_0 - rho_e * v8_2_1);
-            const VT v9_11_0 = QCx * v9_5_0 + WQx * v9_5_1 + (VT)1.0 * oo2e * (v9_2_0 - rho_e * v9_2_1);
-            const VT v10_11_0 = QCx * v10_5_0 + WQx * v10_5_1 + (VT)3.0 * oo2ze * v4_5_1 + (VT)1.0 * oo2e * (v10_2_0 - rho_e * v10_2_1);
-            const VT v11_11_0 = QCx * v11_5_0 + WQx * v11_5_1 + (VT)2.0 * oo2ze * v5_5_1 + (VT)1.0 * oo2e * (v11_2_0 - rho_e * v11_2_1);
-            const VT v12_11_0 = QCx * v12_5_0 + WQx * v12_5_1 + (VT)2.0 * oo2ze * v6_5_1 + (VT)1.0 * oo2e * (v12_2_0 - rho_e * v12_2_1);
-            const VT v13_11_0 = QCx * v13_5_0 + WQx * v13_5_1 + (VT)1.0 * oo2ze * v7_5_1 + (VT)1.0 * oo2e * (v13_2_0 - rho_e * v13_2_1);
-            const VT v14_11_0 = QCx * v14_5_0 + WQx * v14_5_1 + (VT)1.0 * oo2ze * v9_5_1 + (VT)1.0 * oo2e * (v14_2_0 - rho_e * v14_2_1);
-            const VT v15_11_0 = QCx * v15_5_0 + WQx * v15_5_1 + (VT)1.0 * oo2ze * v8_5_1 + (VT)1.0 * oo2e * (v15_2_0 - rho_e * v15_2_1);
-            const VT v16_11_0 = QCx * v16_5_0 + WQx * v16_5_1 + (VT)1.0 * oo2e * (v16_2_0 - rho_e * v16_2_1);
-            const VT v17_11_0 = QCx * v17_5_0 + WQx * v17_5_1 + (VT)1.0 * oo2e * (v17_2_0 - rho_e * v17_2_1);
-            const VT v18_11_0 = QCx * v18_5_0 + WQx * v18_5_1 + (VT)1.0 * oo2e * (v18_2_0 - rho_e * v18_2_1);
-            const VT v19_11_0 = QCx * v19_5_0 + WQx * v19_5_1 + (VT)1.0 * oo2e * (v19_2_0 - rho_e * v19_2_1);
-            const VT v20_11_0 = QCx * v20_5_0 + WQx * v20_5_1 + (VT)4.0 * oo2ze * v10_5_1 + (VT)1.0 * oo2e * (v20_2_0 - rho_e * v20_2_1);
-            const VT v21_11_0 = QCx * v21_5_0 + WQx * v21_5_1 + (VT)3.0 * oo2ze * v11_5_1 + (VT)1.0 * oo2e * (v21_2_0 - rho_e * v21_2_1);
-            const VT v22_11_0 = QCx * v22_5_0 + WQx * v22_5_1 + (VT)3.0 * oo2ze * v12_5_1 + (VT)1.0 * oo2e * (v22_2_0 - rho_e * v22_2_1);
-            const VT v23_11_0 = QCx * v23_5_0 + WQx * v23_5_1 + (VT)2.0 * oo2ze * v13_5_1 + (VT)1.0 * oo2e * (v23_2_0 - rho_e * v23_2_1);
-            const VT v24_11_0 = QCx * v24_5_0 + WQx * v24_5_1 + (VT)2.0 * oo2ze * v15_5_1 + (VT)1.0 * oo2e * (v24_2_0 - rho_e * v24_2_1);
-            const VT v25_11_0 = QCx * v25_5_0 + WQx * v25_5_1 + (VT)2.0 * oo2ze * v14_5_1 + (VT)1.0 * oo2e * (v25_2_0 - rho_e * v25_2_1);
-            const VT v26_11_0 = QCx * v26_5_0 + WQx * v26_5_1 + (VT)1.0 * oo2ze * v16_5_1 + (VT)1.0 * oo2e * (v26_2_0 - rho_e * v26_2_1);
-            const VT v27_11_0 = QCx * v27_5_0 + WQx * v27_5_1 + (VT)1.0 * oo2ze * v17_5_1 + (VT)1.0 * oo2e * (v27_2_0 - rho_e * v27_2_1);
-            const VT v28_11_0 = QCx * v28_5_0 + WQx * v28_5_1 + (VT)1.0 * oo2ze * v18_5_1 + (VT)1.0 * oo2e * (v28_2_0 - rho_e * v28_2_1);
-            const VT v29_11_0 = QCx * v29_5_0 + WQx * v29_5_1 + (VT)1.0 * oo2ze * v19_5_1 + (VT)1.0 * oo2e * (v29_2_0 - rho_e * v29_2_1);
-            const VT v30_11_0 = QCx * v30_5_0 + WQx * v30_5_1 + (VT)1.0 * oo2e * (v30_2_0 - rho_e * v30_2_1);
-            const VT v31_11_0 = QCx * v31_5_0 + WQx * v31_5_1 + (VT)1.0 * oo2e * (v31_2_0 - rho_e * v31_2_1);
-            const VT v32_11_0 = QCx * v32_5_0 + WQx * v32_5_1 + (VT)1.0 * oo2e * (v32_2_0 - rho_e * v32_2_1);
-            const VT v33_11_0 = QCx * v33_5_0 + WQx * v33_5_1 + (VT)1.0 * oo2e * (v33_2_0 - rho_e * v33_2_1);
-            const VT v34_11_0 = QCx * v34_5_0 + WQx * v34_5_1 + (VT)1.0 * oo2e * (v34_2_0 - rho_e * v34_2_1);
-            const VT v4_12_0 = QCx * v4_6_0 + WQx * v4_6_1 + (VT)2.0 * oo2ze * v1_6_1 + (VT)1.0 * oo2e * (v4_3_0 - rho_e * v4_3_1);
-            const VT v5_12_0 = QCx * v5_6_0 + WQx * v5_6_1 + (VT)1.0 * oo2ze * v2_6_1 + (VT)1.0 * oo2e * (v5_3_0 - rho_e * v5_3_1);
-            const VT v6_12_0 = QCx * v6_6_0 + WQx * v6_6_1 + (VT)1.0 * oo2ze * v3_6_1 + (VT)1.0 * oo2e * (v6_3_0 - rho_e * v6_3_1);
-            const VT v7_12_0 = QCx * v7_6_0 + WQx * v7_6_1 + (VT)1.0 * oo2e * (v7_3_0 - rho_e * v7_3_1);
-            const VT v8_12_0 = QCx * v8_6_0 + WQx * v8_6_1 + (VT)1.0 * oo2e * (v8_3_0 - rho_e * v8_3_1);
-            const VT v9_12_0 = QCx * v9_6_0 + WQx * v9_6_1 + (VT)1.0 * oo2e * (v9_3_0 - rho_e * v9_3_1);
-            const VT v10_12_0 = QCx * v10_6_0 + WQx * v10_6_1 + (VT)3.0 * oo2ze * v4_6_1 + (VT)1.0 * oo2e * (v10_3_0 - rho_e * v10_3_1);
-            const VT v11_12_0 = QCx * v11_6_0 + WQx * v11_6_1 + (VT)2.0 * oo2ze * v5_6_1 + (VT)1.0 * oo2e * (v11_3_0 - rho_e * v11_3_1);
-            const VT v12_12_0 = QCx * v12_6_0 + WQx * v12_6_1 + (VT)2.0 * oo2ze * v6_6_1 + (VT)1.0 * oo2e * (v12_3_0 - rho_e * v12_3_1);
-            const VT v13_12_0 = QCx * v13_6_0 + WQx * v13_6_1 + (VT)1.0 * oo2ze * v7_6_1 + (VT)1.0 * oo2e * (v13_3_0 - rho_e * v13_3_1);
-            const VT v14_12_0 = QCx * v14_6_0 + WQx * v14_6_1 + (VT)1.0 * oo2ze * v9_6_1 + (VT)1.0 * oo2e * (v14_3_0 - rho_e * v14_3_1);
-            const VT v15_12_0 = QCx * v15_6_0 + WQx * v15_6_1 + (VT)1.0 * oo2ze * v8_6_1 + (VT)1.0 * oo2e * (v15_3_0 - rho_e * v15_3_1);
-            const VT v16_12_0 = QCx * v16_6_0 + WQx * v16_6_1 + (VT)1.0 * oo2e * (v16_3_0 - rho_e * v16_3_1);
-            const VT v17_12_0 = QCx * v17_6_0 + WQx * v17_6_1 + (VT)1.0 * oo2e * (v17_3_0 - rho_e * v17_3_1);
-            const VT v18_12_0 = QCx * v18_6_0 + WQx * v18_6_1 + (VT)1.0 * oo2e * (v18_3_0 - rho_e * v18_3_1);
-            const VT v19_12_0 = QCx * v19_6_0 + WQx * v19_6_1 + (VT)1.0 * oo2e * (v19_3_0 - rho_e * v19_3_1);
-            const VT v20_12_0 = QCx * v20_6_0 + WQx * v20_6_1 + (VT)4.0 * oo2ze * v10_6_1 + (VT)1.0 * oo2e * (v20_3_0 - rho_e * v20_3_1);
-            const VT v21_12_0 = QCx * v21_6_0 + WQx * v21_6_1 + (VT)3.0 * oo2ze * v11_6_1 + (VT)1.0 * oo2e * (v21_3_0 - rho_e * v21_3_1);
-            const VT v22_12_0 = QCx * v22_6_0 + WQx * v22_6_1 + (VT)3.0 * oo2ze * v12_6_1 + (VT)1.0 * oo2e * (v22_3_0 - rho_e * v22_3_1);
-            const VT v23_12_0 = QCx * v23_6_0 + WQx * v23_6_1 + (VT)2.0 * oo2ze * v13_6_1 + (VT)1.0 * oo2e * (v23_3_0 - rho_e * v23_3_1);
-            const VT v24_12_0 = QCx * v24_6_0 + WQx * v24_6_1 + (VT)2.0 * oo2ze * v15_6_1 + (VT)1.0 * oo2e * (v24_3_0 - rho_e * v24_3_1);
-            const VT v25_12_0 = QCx * v25_6_0 + WQx * v25_6_1 + (VT)2.0 * oo2ze * v14_6_1 + (VT)1.0 * oo2e * (v25_3_0 - rho_e * v25_3_1);
-            const VT v26_12_0 = QCx * v26_6_0 + WQx * v26_6_1 + (VT)1.0 * oo2ze * v16_6_1 + (VT)1.0 * oo2e * (v26_3_0 - rho_e * v26_3_1);
-            const VT v27_12_0 = QCx * v27_6_0 + WQx * v27_6_1 + (VT)1.0 * oo2ze * v17_6_1 + (VT)1.0 * oo2e * (v27_3_0 - rho_e * v27_3_1);
-            const VT v28_12_0 = QCx * v28_6_0 + WQx * v28_6_1 + (VT)1.0 * oo2ze * v18_6_1 + (VT)1.0 * oo2e * (v28_3_0 - rho_e * v28_3_1);
-            const VT v29_12_0 = QCx * v29_6_0 + WQx * v29_6_1 + (VT)1.0 * oo2ze * v19_6_1 + (VT)1.0 * oo2e * (v29_3_0 - rho_e * v29_3_1);
-            const VT v30_12_0 = QCx * v30_6_0 + WQx * v30_6_1 + (VT)1.0 * oo2e * (v30_3_0 - rho_e * v30_3_1);
-            const VT v31_12_0 = QCx * v31_6_0 + WQx * v31_6_1 + (VT)1.0 * oo2e * (v31_3_0 - rho_e * v31_3_1);
-            const VT v32_12_0 = QCx * v32_6_0 + WQx * v32_6_1 + (VT)1.0 * oo2e * (v32_3_0 - rho_e * v32_3_1);
-            const VT v33_12_0 = QCx * v33_6_0 + WQx * v33_6_1 + (VT)1.0 * oo2e * (v33_3_0 - rho_e * v33_3_1);
-            const VT v34_12_0 = QCx * v34_6_0 + WQx * v34_6_1 + (VT)1.0 * oo2e * (v34_3_0 - rho_e * v34_3_1);
-            const VT v4_13_0 = QCy * v4_5_0 + WQy * v4_5_1 + (VT)1.0 * oo2e * (v4_1_0 - rho_e * v4_1_1);
-            const VT v5_13_0 = QCy * v5_5_0 + WQy * v5_5_1 + (VT)1.0 * oo2ze * v1_5_1 + (VT)1.0 * oo2e * (v5_1_0 - rho_e * v5_1_1);
-            const VT v6_13_0 = QCy * v6_5_0 + WQy * v6_5_1 + (VT)1.0 * oo2e * (v6_1_0 - rho_e * v6_1_1);
-            const VT v7_13_0 = QCy * v7_5_0 + WQy * v7_5_1 + (VT)2.0 * oo2ze * v2_5_1 + (VT)1.0 * oo2e * (v7_1_0 - rho_e * v7_1_1);
-            const VT v8_13_0 = QCy * v8_5_0 + WQy * v8_5_1 + (VT)1.0 * oo2ze * v3_5_1 + (VT)1.0 * oo2e * (v8_1_0 - rho_e * v8_1_1);
-            const VT v9_13_0 = QCy * v9_5_0 + WQy * v9_5_1 + (VT)1.0 * oo2e * (v9_1_0 - rho_e * v9_1_1);
-            const VT v10_13_0 = QCy * v10_5_0 + WQy * v10_5_1 + (VT)1.0 * oo2e * (v10_1_0 - rho_e * v10_1_1);
-            const VT v11_13_0 = QCy * v11_5_0 + WQy * v11_5_1 + (VT)1.0 * oo2ze * v4_5_1 + (VT)1.0 * oo2e * (v11_1_0 - rho_e * v11_1_1);
-            const VT v12_13_0 = QCy * v12_5_0 + WQy * v12_5_1 + (VT)1.0 * oo2e * (v12_1_0 - rho_e * v12_1_1);
-            const VT v13_13_0 = QCy * v13_5_0 + WQy * v13_5_1 + (VT)2.0 * oo2ze * v5_5_1 + (VT)1.0 * oo2e * (v13_1_0 - rho_e * v13_1_1);
-            const VT v14_13_0 = QCy * v14_5_0 + WQy * v14_5_1 + (VT)1.0 * oo2e * (v14_1_0 - rho_e * v14_1_1);
-            const VT v15_13_0 = QCy * v15_5_0 + WQy * v15_5_1 + (VT)1.0 * oo2ze * v6_5_1 + (VT)1.0 * oo2e * (v15_1_0 - rho_e * v15_1_1);
-            const VT v16_13_0 = QCy * v16_5_0 + WQy * v16_5_1 + (VT)3.0 * oo2ze * v7_5_1 + (VT)1.0 * oo2e * (v16_1_0 - rho_e * v16_1_1);
-            const VT v17_13_0 = QCy * v17_5_0 + WQy * v17_5_1 + (VT)2.0 * oo2ze * v8_5_1 + (VT)1.0 * oo2e * (v17_1_0 - rho_e * v17_1_1);
-            const VT v18_13_0 = QCy * v18_5_0 + WQy * v18_5_1 + (VT)1.0 * oo2ze * v9_5_1 + (VT)1.0 * oo2e * (v18_1_0 - rho_e * v18_1_1);
-            const VT v19_13_0 = QCy * v19_5_0 + WQy * v19_5_1 + (VT)1.0 * oo2e * (v19_1_0 - rho_e * v19_1_1);
-            const VT v20_13_0 = QCy * v20_5_0 + WQy * v20_5_1 + (VT)1.0 * oo2e * (v20_1_0 - rho_e * v20_1_1);
-            const VT v21_13_0 = QCy * v21_5_0 + WQy * v21_5_1 + (VT)1.0 * oo2ze * v10_5_1 + (VT)1.0 * oo2e * (v21_1_0 - rho_e * v21_1_1);
-            const VT v22_13_0 = QCy * v22_5_0 + WQy * v22_5_1 + (VT)1.0 * oo2e * (v22_1_0 - rho_e * v22_1_1);
-            const VT v23_13_0 = QCy * v23_5_0 + WQy * v23_5_1 + (VT)2.0 * oo2ze * v11_5_1 + (VT)1.0 * oo2e * (v23_1_0 - rho_e * v23_1_1);
-            const VT v24_13_0 = QCy * v24_5_0 + WQy * v24_5_1 + (VT)1.0 * oo2ze * v12_5_1 + (VT)1.0 * oo2e * (v24_1_0 - rho_e * v24_1_1);
-            const VT v25_13_0 = QCy * v25_5_0 + WQy * v25_5_1 + (VT)1.0 * oo2e * (v25_1_0 - rho_e * v25_1_1);
-            const VT v26_13_0 = QCy * v26_5_0 + WQy * v26_5_1 + (VT)3.0 * oo2ze * v13_5_1 + (VT)1.0 * oo2e * (v26_1_0 - rho_e * v26_1_1);
-            const VT v27_13_0 = QCy * v27_5_0 + WQy * v27_5_1 + (VT)2.0 * oo2ze * v15_5_1 + (VT)1.0 * oo2e * (v27_1_0 - rho_e * v27_1_1);
-            const VT v28_13_0 = QCy * v28_5_0 + WQy * v28_5_1 + (VT)1.0 * oo2ze * v14_5_1 + (VT)1.0 * oo2e * (v28_1_0 - rho_e * v28_1_1);
-            const VT v29_13_0 = QCy * v29_5_0 + WQy * v29_5_1 + (VT)1.0 * oo2e * (v29_1_0 - rho_e * v29_1_1);
-            const VT v30_13_0 = QCy * v30_5_0 + WQy * v30_5_1 + (VT)4.0 * oo2ze * v16_5_1 + (VT)1.0 * oo2e * (v30_1_0 - rho_e * v30_1_1);
-            const VT v31_13_0 = QCy * v31_5_0 + WQy * v31_5_1 + (VT)3.0 * oo2ze * v17_5_1 + (VT)1.0 * oo2e * (v31_1_0 - rho_e * v31_1_1);
-            const VT v32_13_0 = QCy * v32_5_0 + WQy * v32_5_1 + (VT)2.0 * oo2ze * v18_5_1 + (VT)1.0 * oo2e * (v32_1_0 - rho_e * v32_1_1);
-            const VT v33_13_0 = QCy * v33_5_0 + WQy * v33_5_1 + (VT)1.0 * oo2ze * v19_5_1 + (VT)1.0 * oo2e * (v33_1_0 - rho_e * v33_1_1);
-            const VT v34_13_0 = QCy * v34_5_0 + WQy * v34_5_1 + (VT)1.0 * oo2e * (v34_1_0 - rho_e * v34_1_1);
-            const VT v4_14_0 = QCz * v4_6_0 + WQz * v4_6_1 + (VT)1.0 * oo2e * (v4_1_0 - rho_e * v4_1_1);
-            const VT v5_14_0 = QCz * v5_6_0 + WQz * v5_6_1 + (VT)1.0 * oo2e * (v5_1_0 - rho_e * v5_1_1);
-            const VT v6_14_0 = QCz * v6_6_0 + WQz * v6_6_1 + (VT)1.0 * oo2ze * v1_6_1 + (VT)1.0 * oo2e * (v6_1_0 - rho_e * v6_1_1);
-            const VT v7_14_0 = QCz * v7_6_0 + WQz * v7_6_1 + (VT)1.0 * oo2e * (v7_1_0 - rho_e * v7_1_1);
-            const VT v8_14_0 = QCz * v8_6_0 + WQz * v8_6_1 + (VT)1.0 * oo2ze * v2_6_1 + (VT)1.0 * oo2e * (v8_1_0 - rho_e * v8_1_1);
-            const VT v9_14_0 = QCz * v9_6_0 + WQz * v9_6_1 + (VT)2.0 * oo2ze * v3_6_1 + (VT)1.0 * oo2e * (v9_1_0 - rho_e * v9_1_1);
-            const VT v10_14_0 = QCz * v10_6_0 + WQz * v10_6_1 + (VT)1.0 * oo2e * (v10_1_0 - rho_e * v10_1_1);
-            const VT v11_14_0 = QCz * v11_6_0 + WQz * v11_6_1 + (VT)1.0 * oo2e * (v11_1_0 - rho_e * v11_1_1);
-            const VT v12_14_0 = QCz * v12_6_0 + WQz * v12_6_1 + (VT)1.0 * oo2ze * v4_6_1 + (VT)1.0 * oo2e * (v12_1_0 - rho_e * v12_1_1);
-            const VT v13_14_0 = QCz * v13_6_0 + WQz * v13_6_1 + (VT)1.0 * oo2e * (v13_1_0 - rho_e * v13_1_1);
-            const VT v14_14_0 = QCz * v14_6_0 + WQz * v14_6_1 + (VT)2.0 * oo2ze * v6_6_1 + (VT)1.0 * oo2e * (v14_1_0 - rho_e * v14_1_1);
-            const VT v15_14_0 = QCz * v15_6_0 + WQz * v15_6_1 + (VT)1.0 * oo2ze * v5_6_1 + (VT)1.0 * oo2e * (v15_1_0 - rho_e * v15_1_1);
-            const VT v16_14_0 = QCz * v16_6_0 + WQz * v16_6_1 + (VT)1.0 * oo2e * (v16_1_0 - rho_e * v16_1_1);
-            const VT v17_14_0 = QCz * v17_6_0 + WQz * v17_6_1 + (VT)1.0 * oo2ze * v7_6_1 + (VT)1.0 * oo2e * (v17_1_0 - rho_e * v17_1_1);
-            const VT v18_14_0 = QCz * v18_6_0 + WQz * v18_6_1 + (VT)2.0 * oo2ze * v8_6_1 + (VT)1.0 * oo2e * (v18_1_0 - rho_e * v18_1_1);
-            const VT v19_14_0 = QCz * v19_6_0 + WQz * v19_6_1 + (VT)3.0 * oo2ze * v9_6_1 + (VT)1.0 * oo2e * (v19_1_0 - rho_e * v19_1_1);
-            const VT v20_14_0 = QCz * v20_6_0 + WQz * v20_6_1 + (VT)1.0 * oo2e * (v20_1_0 - rho_e * v20_1_1);
-            const VT v21_14_0 = QCz * v21_6_0 + WQz * v21_6_1 + (VT)1.0 * oo2e * (v21_1_0 - rho_e * v21_1_1);
-            const VT v22_14_0 = QCz * v22_6_0 + WQz * v22_6_1 + (VT)1.0 * oo2ze * v10_6_1 + (VT)1.0 * oo2e * (v22_1_0 - rho_e * v22_1_1);
-            const VT v23_14_0 = QCz * v23_6_0 + WQz * v23_6_1 + (VT)1.0 * oo2e * (v23_1_0 - rho_e * v23_1_1);
-            const VT v24_14_0 = QCz * v24_6_0 + WQz * v24_6_1 + (VT)1.0 * oo2ze * v11_6_1 + (VT)1.0 * oo2e * (v24_1_0 - rho_e * v24_1_1);
-            const VT v25_14_0 = QCz * v25_6_0 + WQz * v25_6_1 + (VT)2.0 * oo2ze * v12_6_1 + (VT)1.0 * oo2e * (v25_1_0 - rho_e * v25_1_1);
-            const VT v26_14_0 = QCz * v26_6_0 + WQz * v26_6_1 + (VT)1.0 * oo2e * (v26_1_0 - rho_e * v26_1_1);
-            const VT v27_14_0 = QCz * v27_6_0 + WQz * v27_6_1 + (VT)1.0 * oo2ze * v13_6_1 + (VT)1.0 * oo2e * (v27_1_0 - rho_e * v27_1_1);
-            const VT v28_14_0 = QCz * v28_6_0 + WQz * v28_6_1 + (VT)2.0 * oo2ze * v15_6_1 + (VT)1.0 * oo2e * (v28_1_0 - rho_e * v28_1_1);
-            const VT v29_14_0 = QCz * v29_6_0 + WQz * v29_6_1 + (VT)3.0 * oo2ze * v14_6_1 + (VT)1.0 * oo2e * (v29_1_0 - rho_e * v29_1_1);
-            const VT v30_14_0 = QCz * v30_6_0 + WQz * v30_6_1 + (VT)1.0 * oo2e * (v30_1_0 - rho_e * v30_1_1);
-            const VT v31_14_0 = QCz * v31_6_0 + WQz * v31_6_1 + (VT)1.0 * oo2ze * v16_6_1 + (VT)1.0 * oo2e * (v31_1_0 - rho_e * v31_1_1);
-            const VT v32_14_0 = QCz * v32_6_0 + WQz * v32_6_1 + (VT)2.0 * oo2ze * v17_6_1 + (VT)1.0 * oo2e * (v32_1_0 - rho_e * v32_1_1);
-            const VT v33_14_0 = QCz * v33_6_0 + WQz * v33_6_1 + (VT)3.0 * oo2ze * v18_6_1 + (VT)1.0 * oo2e * (v33_1_0 - rho_e * v33_1_1);
-            const VT v34_14_0 = QCz * v34_6_0 + WQz * v34_6_1 + (VT)4.0 * oo2ze * v19_6_1 + (VT)1.0 * oo2e * (v34_1_0 - rho_e * v34_1_1);
-            const VT v4_15_0 = QCx * v4_8_0 + WQx * v4_8_1 + (VT)2.0 * oo2ze * v1_8_1;
-            const VT v5_15_0 = QCx * v5_8_0 + WQx * v5_8_1 + (VT)1.0 * oo2ze * v2_8_1;
-            const VT v6_15_0 = QCx * v6_8_0 + WQx * v6_8_1 + (VT)1.0 * oo2ze * v3_8_1;
-            const VT v7_15_0 = QCx * v7_8_0 + WQx * v7_8_1;
-            const VT v8_15_0 = QCx * v8_8_0 + WQx * v8_8_1;
-            const VT v9_15_0 = QCx * v9_8_0 + WQx * v9_8_1;
-            const VT v10_15_0 = QCx * v10_8_0 + WQx * v10_8_1 + (VT)3.0 * oo2ze * v4_8_1;
-            const VT v11_15_0 = QCx * v11_8_0 + WQx * v11_8_1 + (VT)2.0 * oo2ze * v5_8_1;
-            const VT v12_15_0 = QCx * v12_8_0 + WQx * v12_8_1 + (VT)2.0 * oo2ze * v6_8_1;
-            const VT v13_15_0 = QCx * v13_8_0 + WQx * v13_8_1 + (VT)1.0 * oo2ze * v7_8_1;
-            const VT v14_15_0 = QCx * v14_8_0 + WQx * v14_8_1 + (VT)1.0 * oo2ze * v9_8_1;
-            const VT v15_15_0 = QCx * v15_8_0 + WQx * v15_8_1 + (VT)1.0 * oo2ze * v8_8_1;
-            const VT v16_15_0 = QCx * v16_8_0 + WQx * v16_8_1;
-            const VT v17_15_0 = QCx * v17_8_0 + WQx * v17_8_1;
-            const VT v18_15_0 = QCx * v18_8_0 + WQx * v18_8_1;
-            const VT v19_15_0 = QCx * v19_8_0 + WQx * v19_8_1;
-            const VT v20_15_0 = QCx * v20_8_0 + WQx * v20_8_1 + (VT)4.0 * oo2ze * v10_8_1;
-            const VT v21_15_0 = QCx * v21_8_0 + WQx * v21_8_1 + (VT)3.0 * oo2ze * v11_8_1;
-            const VT v22_15_0 = QCx * v22_8_0 + WQx * v22_8_1 + (VT)3.0 * oo2ze * v12_8_1;
-            const VT v23_15_0 = QCx * v23_8_0 + WQx * v23_8_1 + (VT)2.0 * oo2ze * v13_8_1;
-            const VT v24_15_0 = QCx * v24_8_0 + WQx * v24_8_1 + (VT)2.0 * oo2ze * v15_8_1;
-            const VT v25_15_0 = QCx * v25_8_0 + WQx * v25_8_1 + (VT)2.0 * oo2ze * v14_8_1;
-            const VT v26_15_0 = QCx * v26_8_0 + WQx * v26_8_1 + (VT)1.0 * oo2ze * v16_8_1;
-            const VT v27_15_0 = QCx * v27_8_0 + WQx * v27_8_1 + (VT)1.0 * oo2ze * v17_8_1;
-            const VT v28_15_0 = QCx * v28_8_0 + WQx * v28_8_1 + (VT)1.0 * oo2ze * v18_8_1;
-            const VT v29_15_0 = QCx * v29_8_0 + WQx * v29_8_1 + (VT)1.0 * oo2ze * v19_8_1;
-            const VT v30_15_0 = QCx * v30_8_0 + WQx * v30_8_1;
-            const VT v31_15_0 = QCx * v31_8_0 + WQx * v31_8_1;
-            const VT v32_15_0 = QCx * v32_8_0 + WQx * v32_8_1;
-            const VT v33_15_0 = QCx * v33_8_0 + WQx * v33_8_1;
-            const VT v34_15_0 = QCx * v34_8_0 + WQx * v34_8_1;
-            const VT v4_16_0 = QCy * v4_7_0 + WQy * v4_7_1 + (VT)2.0 * oo2e * (v4_2_0 - rho_e * v4_2_1);
-            const VT v5_16_0 = QCy * v5_7_0 + WQy * v5_7_1 + (VT)1.0 * oo2ze * v1_7_1 + (VT)2.0 * oo2e * (v5_2_0 - rho_e * v5_2_1);
-            const VT v6_16_0 = QCy * v6_7_0 + WQy * v6_7_1 + (VT)2.0 * oo2e * (v6_2_0 - rho_e * v6_2_1);
-            const VT v7_16_0 = QCy * v7_7_0 + WQy * v7_7_1 + (VT)2.0 * oo2ze * v2_7_1 + (VT)2.0 * oo2e * (v7_2_0 - rho_e * v7_2_1);
-            const VT v8_16_0 = QCy * v8_7_0 + WQy * v8_7_1 + (VT)1.0 * oo2ze * v3_7_1 + (VT)2.0 * oo2e * (v8_2_0 - rho_e * v8_2_1);
-            const VT v9_16_0 = QCy * v9_7_0 + WQy * v9_7_1 + (VT)2.0 * oo2e * (v9_2_0 - rho_e * v9_2_1);
-            const VT v10_16_0 = QCy * v10_7_0 + WQy * v10_7_1 + (VT)2.0 * oo2e * (v10_2_0 - rho_e * v10_2_1);
-            const VT v11_16_0 = QCy * v11_7_0 + WQy * v11_7_1 + (VT)1.0 * oo2ze * v4_7_1 + (VT)2.0 * oo2e * (v11_2_0 - rho_e * v11_2_1);
-            const VT v12_16_0 = QCy * v12_7_0 + WQy * v12_7_1 + (VT)2.0 * oo2e * (v12_2_0 - rho_e * v12_2_1);
-            const VT v13_16_0 = QCy * v13_7_0 + WQy * v13_7_1 + (VT)2.0 * oo2ze * v5_7_1 + (VT)2.0 * oo2e * (v13_2_0 - rho_e * v13_2_1);
-            const VT v14_16_0 = QCy * v14_7_0 + WQy * v14_7_1 + (VT)2.0 * oo2e * (v14_2_0 - rho_e * v14_2_1);
-            const VT v15_16_0 = QCy * v15_7_0 + WQy * v15_7_1 + (VT)1.0 * oo2ze * v6_7_1 + (VT)2.0 * oo2e * (v15_2_0 - rho_e * v15_2_1);
-            const VT v16_16_0 = QCy * v16_7_0 + WQy * v16_7_1 + (VT)3.0 * oo2ze * v7_7_1 + (VT)2.0 * oo2e * (v16_2_0 - rho_e * v16_2_1);
-            const VT v17_16_0 = QCy * v17_7_0 + WQy * v17_7_1 + (VT)2.0 * oo2ze * v8_7_1 + (VT)2.0 * oo2e * (v17_2_0 - rho_e * v17_2_1);
-            const VT v18_16_0 = QCy * v18_7_0 + WQy * v18_7_1 + (VT)1.0 * oo2ze * v9_7_1 + (VT)2.0 * oo2e * (v18_2_0 - rho_e * v18_2_1);
-            const VT v19_16_0 = QCy * v19_7_0 + WQy * v19_7_1 + (VT)2.0 * oo2e * (v19_2_0 - rho_e * v19_2_1);
-            const VT v20_16_0 = QCy * v20_7_0 + WQy * v20_7_1 + (VT)2.0 * oo2e * (v20_2_0 - rho_e * v20_2_1);
-            const VT v21_16_0 = QCy * v21_7_0 + WQy * v21_7_1 + (VT)1.0 * oo2ze * v10_7_1 + (VT)2.0 * oo2e * (v21_2_0 - rho_e * v21_2_1);
-            const VT v22_16_0 = QCy * v22_7_0 + WQy * v22_7_1 + (VT)2.0 * oo2e * (v22_2_0 - rho_e * v22_2_1);
-            const VT v23_16_0 = QCy * v23_7_0 + WQy * v23_7_1 + (VT)2.0 * oo2ze * v11_7_1 + (VT)2.0 * oo2e * (v23_2_0 - rho_e * v23_2_1);
-            const VT v24_16_0 = QCy * v24_7_0 + WQy * v24_7_1 + (VT)1.0 * oo2ze * v12_7_1 + (VT)2.0 * oo2e * (v24_2_0 - rho_e * v24_2_1);
-            const VT v25_16_0 = QCy * v25_7_0 + WQy * v25_7_1 + (VT)2.0 * oo2e * (v25_2_0 - rho_e * v25_2_1);
-            const VT v26_16_0 = QCy * v26_7_0 + WQy * v26_7_1 + (VT)3.0 * oo2ze * v13_7_1 + (VT)2.0 * oo2e * (v26_2_0 - rho_e * v26_2_1);
-            const VT v27_16_0 = QCy * v27_7_0 + WQy * v27_7_1 + (VT)2.0 * oo2ze * v15_7_1 + (VT)2.0 * oo2e * (v27_2_0 - rho_e * v27_2_1);
-            const VT v28_16_0 = QCy * v28_7_0 + WQy * v28_7_1 + (VT)1.0 * oo2ze * v14_7_1 + (VT)2.0 * oo2e * (v28_2_0 - rho_e * v28_2_1);
-            const VT v29_16_0 = QCy * v29_7_0 + WQy * v29_7_1 + (VT)2.0 * oo2e * (v29_2_0 - rho_e * v29_2_1);
-            const VT v30_16_0 = QCy * v30_7_0 + WQy * v30_7_1 + (VT)4.0 * oo2ze * v16_7_1 + (VT)2.0 * oo2e * (v30_2_0 - rho_e * v30_2_1);
-            const VT v31_16_0 = QCy * v31_7_0 + WQy * v31_7_1 + (VT)3.0 * oo2ze * v17_7_1 + (VT)2.0 * oo2e * (v31_2_0 - rho_e * v31_2_1);
-            const VT v32_16_0 = QCy * v32_7_0 + WQy * v32_7_1 + (VT)2.0 * oo2ze * v18_7_1 + (VT)2.0 * oo2e * (v32_2_0 - rho_e * v32_2_1);
-            const VT v33_16_0 = QCy * v33_7_0 + WQy * v33_7_1 + (VT)1.0 * oo2ze * v19_7_1 + (VT)2.0 * oo2e * (v33_2_0 - rho_e * v33_2_1);
-            const VT v34_16_0 = QCy * v34_7_0 + WQy * v34_7_1 + (VT)2.0 * oo2e * (v34_2_0 - rho_e * v34_2_1);
-            const VT v4_17_0 = QCy * v4_8_0 + WQy * v4_8_1 + (VT)1.0 * oo2e * (v4_3_0 - rho_e * v4_3_1);
-            const VT v5_17_0 = QCy * v5_8_0 + WQy * v5_8_1 + (VT)1.0 * oo2ze * v1_8_1 + (VT)1.0 * oo2e * (v5_3_0 - rho_e * v5_3_1);
-            const VT v6_17_0 = QCy * v6_8_0 + WQy * v6_8_1 + (VT)1.0 * oo2e * (v6_3_0 - rho_e * v6_3_1);
-            const VT v7_17_0 = QCy * v7_8_0 + WQy * v7_8_1 + (VT)2.0 * oo2ze * v2_8_1 + (VT)1.0 * oo2e * (v7_3_0 - rho_e * v7_3_1);
-            const VT v8_17_0 = QCy * v8_8_0 + WQy * v8_8_1 + (VT)1.0 * oo2ze * v3_8_1 + (VT)1.0 * oo2e * (v8_3_0 - rho_e * v8_3_1);
-            const VT v9_17_0 = QCy * v9_8_0 + WQy * v9_8_1 + (VT)1.0 * oo2e * (v9_3_0 - rho_e * v9_3_1);
-            const VT v10_17_0 = QCy * v10_8_0 + WQy * v10_8_1 + (VT)1.0 * oo2e * (v10_3_0 - rho_e * v10_3_1);
-            const VT v11_17_0 = QCy * v11_8_0 + WQy * v11_8_1 + (VT)1.0 * oo2ze * v4_8_1 + (VT)1.0 * oo2e * (v11_3_0 - rho_e * v11_3_1);
-            const VT v12_17_0 = QCy * v12_8_0 + WQy * v12_8_1 + (VT)1.0 * oo2e * (v12_3_0 - rho_e * v12_3_1);
-            const VT v13_17_0 = QCy * v13_8_0 + WQy * v13_8_1 + (VT)2.0 * oo2ze * v5_8_1 + (VT)1.0 * oo2e * (v13_3_0 - rho_e * v13_3_1);
-            const VT v14_17_0 = QCy * v14_8_0 + WQy * v14_8_1 + (VT)1.0 * oo2e * (v14_3_0 - rho_e * v14_3_1);
-            const VT v15_17_0 = QCy * v15_8_0 + WQy * v15_8_1 + (VT)1.0 * oo2ze * v6_8_1 + (VT)1.0 * oo2e * (v15_3_0 - rho_e * v15_3_1);
-            const VT v16_17_0 = QCy * v16_8_0 + WQy * v16_8_1 + (VT)3.0 * oo2ze * v7_8_1 + (VT)1.0 * oo2e * (v16_3_0 - rho_e * v16_3_1);
-            const VT v17_17_0 = QCy * v17_8_0 + WQy * v17_8_1 + (VT)2.0 * oo2ze * v8_8_1 + (VT)1.0 * oo2e * (v17_3_0 - rho_e * v17_3_1);
-            const VT v18_17_0 = QCy * v18_8_0 + WQy * v18_8_1 + (VT)1.0 * oo2ze * v9_8_1 + (VT)1.0 * oo2e * (v18_3_0 - rho_e * v18_3_1);
-            const VT v19_17_0 = QCy * v19_8_0 + WQy * v19_8_1 + (VT)1.0 * oo2e * (v19_3_0 - rho_e * v19_3_1);
-            const VT v20_17_0 = QCy * v20_8_0 + WQy * v20_8_1 + (VT)1.0 * oo2e * (v20_3_0 - rho_e * v20_3_1);
-            const VT v21_17_0 = QCy * v21_8_0 + WQy * v21_8_1 + (VT)1.0 * oo2ze * v10_8_1 + (VT)1.0 * oo2e * (v21_3_0 - rho_e * v21_3_1);
-            const VT v22_17_0 = QCy * v22_8_0 + WQy * v22_8_1 + (VT)1.0 * oo2e * (v22_3_0 - rho_e * v22_3_1);
-            const VT v23_17_0 = QCy * v23_8_0 + WQy * v23_8_1 + (VT)2.0 * oo2ze * v11_8_1 + (VT)1.0 * oo2e * (v23_3_0 - rho_e * v23_3_1);
-            const VT v24_17_0 = QCy * v24_8_0 + WQy * v24_8_1 + (VT)1.0 * oo2ze * v12_8_1 + (VT)1.0 * oo2e * (v24_3_0 - rho_e * v24_3_1);
-            const VT v25_17_0 = QCy * v25_8_0 + WQy * v25_8_1 + (VT)1.0 * oo2e * (v25_3_0 - rho_e * v25_3_1);
-            const VT v26_17_0 = QCy * v26_8_0 + WQy * v26_8_1 + (VT)3.0 * oo2ze * v13_8_1 + (VT)1.0 * oo2e * (v26_3_0 - rho_e * v26_3_1);
-            const VT v27_17_0 = QCy * v27_8_0 + WQy * v27_8_1 + (VT)2.0 * oo2ze * v15_8_1 + (VT)1.0 * oo2e * (v27_3_0 - rho_e * v27_3_1);
-            const VT v28_17_0 = QCy * v28_8_0 + WQy * v28_8_1 + (VT)1.0 * oo2ze * v14_8_1 + (VT)1.0 * oo2e * (v28_3_0 - rho_e * v28_3_1);
-            const VT v29_17_0 = QCy * v29_8_0 + WQy * v29_8_1 + (VT)1.0 * oo2e * (v29_3_0 - rho_e * v29_3_1);
-            const VT v30_17_0 = QCy * v30_8_0 + WQy * v30_8_1 + (VT)4.0 * oo2ze * v16_8_1 + (VT)1.0 * oo2e * (v30_3_0 - rho_e * v30_3_1);
-            const VT v31_17_0 = QCy * v31_8_0 + WQy * v31_8_1 + (VT)3.0 * oo2ze * v17_8_1 + (VT)1.0 * oo2e * (v31_3_0 - rho_e * v31_3_1);
-            const VT v32_17_0 = QCy * v32_8_0 + WQy * v32_8_1 + (VT)2.0 * oo2ze * v18_8_1 + (VT)1.0 * oo2e * (v32_3_0 - rho_e * v32_3_1);
-            const VT v33_17_0 = QCy * v33_8_0 + WQy * v33_8_1 + (VT)1.0 * oo2ze * v19_8_1 + (VT)1.0 * oo2e * (v33_3_0 - rho_e * v33_3_1);
-            const VT v34_17_0 = QCy * v34_8_0 + WQy * v34_8_1 + (VT)1.0 * oo2e * (v34_3_0 - rho_e * v34_3_1);
-            const VT v4_18_0 = QCz * v4_8_0 + WQz * v4_8_1 + (VT)1.0 * oo2e * (v4_2_0 - rho_e * v4_2_1);
-            const VT v5_18_0 = QCz * v5_8_0 + WQz * v5_8_1 + (VT)1.0 * oo2e * (v5_2_0 - rho_e * v5_2_1);
-            const VT v6_18_0 = QCz * v6_8_0 + WQz * v6_8_1 + (VT)1.0 * oo2ze * v1_8_1 + (VT)1.0 * oo2e * (v6_2_0 - rho_e * v6_2_1);
-            const VT v7_18_0 = QCz * v7_8_0 + WQz * v7_8_1 + (VT)1.0 * oo2e * (v7_2_0 - rho_e * v7_2_1);
-            const VT v8_18_0 = QCz * v8_8_0 + WQz * v8_8_1 + (VT)1.0 * oo2ze * v2_8_1 + (VT)1.0 * oo2e * (v8_2_0 - rho_e * v8_2_1);
-            const VT v9_18_0 = QCz * v9_8_0 + WQz * v9_8_1 + (VT)2.0 * oo2ze * v3_8_1 + (VT)1.0 * oo2e * (v9_2_0 - rho_e * v9_2_1);
-            const VT v10_18_0 = QCz * v10_8_0 + WQz * v10_8_1 + (VT)1.0 * oo2e * (v10_2_0 - rho_e * v10_2_1);
-            const VT v11_18_0 = QCz * v11_8_0 + WQz * v11_8_1 + (VT)1.0 * oo2e * (v11_2_0 - rho_e * v11_2_1);
-            const VT v12_18_0 = QCz * v12_8_0 + WQz * v12_8_1 + (VT)1.0 * oo2ze * v4_8_1 + (VT)1.0 * oo2e * (v12_2_0 - rho_e * v12_2_1);
-            const VT v13_18_0 = QCz * v13_8_0 + WQz * v13_8_1 + (VT)1.0 * oo2e * (v13_2_0 - rho_e * v13_2_1);
-            const VT v14_18_0 = QCz * v14_8_0 + WQz * v14_8_1 + (VT)2.0 * oo2ze * v6_8_1 + (VT)1.0 * oo2e * (v14_2_0 - rho_e * v14_2_1);
-            const VT v15_18_0 = QCz * v15_8_0 + WQz * v15_8_1 + (VT)1.0 * oo2ze * v5_8_1 + (VT)1.0 * oo2e * (v15_2_0 - rho_e * v15_2_1);
-            const VT v16_18_0 = QCz * v16_8_0 + WQz * v16_8_1 + (VT)1.0 * oo2e * (v16_2_0 - rho_e * v16_2_1);
-            const VT v17_18_0 = QCz * v17_8_0 + WQz * v17_8_1 + (VT)1.0 * oo2ze * v7_8_1 + (VT)1.0 * oo2e * (v17_2_0 - rho_e * v17_2_1);
-            const VT v18_18_0 = QCz * v18_8_0 + WQz * v18_8_1 + (VT)2.0 * oo2ze * v8_8_1 + (VT)1.0 * oo2e * (v18_2_0 - rho_e * v18_2_1);
-            const VT v19_18_0 = QCz * v19_8_0 + WQz * v19_8_1 + (VT)3.0 * oo2ze * v9_8_1 + (VT)1.0 * oo2e * (v19_2_0 - rho_e * v19_2_1);
-            const VT v20_18_0 = QCz * v20_8_0 + WQz * v20_8_1 + (VT)1.0 * oo2e * (v20_2_0 - rho_e * v20_2_1);
-            const VT v21_18_0 = QCz * v21_8_0 + WQz * v21_8_1 + (VT)1.0 * oo2e * (v21_2_0 - rho_e * v21_2_1);
-            const VT v22_18_0 = QCz * v22_8_0 + WQz * v22_8_1 + (VT)1.0 * oo2ze * v10_8_1 + (VT)1.0 * oo2e * (v22_2_0 - rho_e * v22_2_1);
-            const VT v23_18_0 = QCz * v23_8_0 + WQz * v23_8_1 + (VT)1.0 * oo2e * (v23_2_0 - rho_e * v23_2_1);
-            const VT v24_18_0 = QCz * v24_8_0 + WQz * v24_8_1 + (VT)1.0 * oo2ze * v11_8_1 + (VT)1.0 * oo2e * (v24_2_0 - rho_e * v24_2_1);
-            const VT v25_18_0 = QCz * v25_8_0 + WQz * v25_8_1 + (VT)2.0 * oo2ze * v12_8_1 + (VT)1.0 * oo2e * (v25_2_0 - rho_e * v25_2_1);
-            const VT v26_18_0 = QCz * v26_8_0 + WQz * v26_8_1 + (VT)1.0 * oo2e * (v26_2_0 - rho_e * v26_2_1);
-            const VT v27_18_0 = QCz * v27_8_0 + WQz * v27_8_1 + (VT)1.0 * oo2ze * v13_8_1 + (VT)1.0 * oo2e * (v27_2_0 - rho_e * v27_2_1);
-            const VT v28_18_0 = QCz * v28_8_0 + WQz * v28_8_1 + (VT)2.0 * oo2ze * v15_8_1 + (VT)1.0 * oo2e * (v28_2_0 - rho_e * v28_2_1);
-            const VT v29_18_0 = QCz * v29_8_0 + WQz * v29_8_1 + (VT)3.0 * oo2ze * v14_8_1 + (VT)1.0 * oo2e * (v29_2_0 - rho_e * v29_2_1);
-            const VT v30_18_0 = QCz * v30_8_0 + WQz * v30_8_1 + (VT)1.0 * oo2e * (v30_2_0 - rho_e * v30_2_1);
-            const VT v31_18_0 = QCz * v31_8_0 + WQz * v31_8_1 + (VT)1.0 * oo2ze * v16_8_1 + (VT)1.0 * oo2e * (v31_2_0 - rho_e * v31_2_1);
-            const VT v32_18_0 = QCz * v32_8_0 + WQz * v32_8_1 + (VT)2.0 * oo2ze * v17_8_1 + (VT)1.0 * oo2e * (v32_2_0 - rho_e * v32_2_1);
-            const VT v33_18_0 = QCz * v33_8_0 + WQz * v33_8_1 + (VT)3.0 * oo2ze * v18_8_1 + (VT)1.0 * oo2e * (v33_2_0 - rho_e * v33_2_1);
-            const VT v34_18_0 = QCz * v34_8_0 + WQz * v34_8_1 + (VT)4.0 * oo2ze * v19_8_1 + (VT)1.0 * oo2e * (v34_2_0 - rho_e * v34_2_1);
-            const VT v4_19_0 = QCz * v4_9_0 + WQz * v4_9_1 + (VT)2.0 * oo2e * (v4_3_0 - rho_e * v4_3_1);
-            const VT v5_19_0 = QCz * v5_9_0 + WQz * v5_9_1 + (VT)2.0 * oo2e * (v5_3_0 - rho_e * v5_3_1);
-            const VT v6_19_0 = QCz * v6_9_0 + WQz * v6_9_1 + (VT)1.0 * oo2ze * v1_9_1 + (VT)2.0 * oo2e * (v6_3_0 - rho_e * v6_3_1);
-            const VT v7_19_0 = QCz * v7_9_0 + WQz * v7_9_1 + (VT)2.0 * oo2e * (v7_3_0 - rho_e * v7_3_1);
-            const VT v8_19_0 = QCz * v8_9_0 + WQz * v8_9_1 + (VT)1.0 * oo2ze * v2_9_1 + (VT)2.0 * oo2e * (v8_3_0 - rho_e * v8_3_1);
-            const VT v9_19_0 = QCz * v9_9_0 + WQz * v9_9_1 + (VT)2.0 * oo2ze * v3_9_1 + (VT)2.0 * oo2e * (v9_3_0 - rho_e * v9_3_1);
-            const VT v10_19_0 = QCz * v10_9_0 + WQz * v10_9_1 + (VT)2.0 * oo2e * (v10_3_0 - rho_e * v10_3_1);
-            const VT v11_19_0 = QCz * v11_9_0 + WQz * v11_9_1 + (VT)2.0 * oo2e * (v11_3_0 - rho_e * v11_3_1);
-            const VT v12_19_0 = QCz * v12_9_0 + WQz * v12_9_1 + (VT)1.0 * oo2ze * v4_9_1 + (VT)2.0 * oo2e * (v12_3_0 - rho_e * v12_3_1);
-            const VT v13_19_0 = QCz * v13_9_0 + WQz * v13_9_1 + (VT)2.0 * oo2e * (v13_3_0 - rho_e * v13_3_1);
-            const VT v14_19_0 = QCz * v14_9_0 + WQz * v14_9_1 + (VT)2.0 * oo2ze * v6_9_1 + (VT)2.0 * oo2e * (v14_3_0 - rho_e * v14_3_1);
-            const VT v15_19_0 = QCz * v15_9_0 + WQz * v15_9_1 + (VT)1.0 * oo2ze * v5_9_1 + (VT)2.0 * oo2e * (v15_3_0 - rho_e * v15_3_1);
-            const VT v16_19_0 = QCz * v16_9_0 + WQz * v16_9_1 + (VT)2.0 * oo2e * (v16_3_0 - rho_e * v16_3_1);
-            const VT v17_19_0 = QCz * v17_9_0 + WQz * v17_9_1 + (VT)1.0 * oo2ze * v7_9_1 + (VT)2.0 * oo2e * (v17_3_0 - rho_e * v17_3_1);
-            const VT v18_19_0 = QCz * v18_9_0 + WQz * v18_9_1 + (VT)2.0 * oo2ze * v8_9_1 + (VT)2.0 * oo2e * (v18_3_0 - rho_e * v18_3_1);
-            const VT v19_19_0 = QCz * v19_9_0 + WQz * v19_9_1 + (VT)3.0 * oo2ze * v9_9_1 + (VT)2.0 * oo2e * (v19_3_0 - rho_e * v19_3_1);
-            const VT v20_19_0 = QCz * v20_9_0 + WQz * v20_9_1 + (VT)2.0 * oo2e * (v20_3_0 - rho_e * v20_3_1);
-            const VT v21_19_0 = QCz * v21_9_0 + WQz * v21_9_1 + (VT)2.0 * oo2e * (v21_3_0 - rho_e * v21_3_1);
-            const VT v22_19_0 = QCz * v22_9_0 + WQz * v22_9_1 + (VT)1.0 * oo2ze * v10_9_1 + (VT)2.0 * oo2e * (v22_3_0 - rho_e * v22_3_1);
-            const VT v23_19_0 = QCz * v23_9_0 + WQz * v23_9_1 + (VT)2.0 * oo2e * (v23_3_0 - rho_e * v23_3_1);
-            const VT v24_19_0 = QCz * v24_9_0 + WQz * v24_9_1 + (VT)1.0 * oo2ze * v11_9_1 + (VT)2.0 * oo2e * (v24_3_0 - rho_e * v24_3_1);
-            const VT v25_19_0 = QCz * v25_9_0 + WQz * v25_9_1 + (VT)2.0 * oo2ze * v12_9_1 + (VT)2.0 * oo2e * (v25_3_0 - rho_e * v25_3_1);
-            const VT v26_19_0 = QCz * v26_9_0 + WQz * v26_9_1 + (VT)2.0 * oo2e * (v26_3_0 - rho_e * v26_3_1);
-            const VT v27_19_0 = QCz * v27_9_0 + WQz * v27_9_1 + (VT)1.0 * oo2ze * v13_9_1 + (VT)2.0 * oo2e * (v27_3_0 - rho_e * v27_3_1);
-            const VT v28_19_0 = QCz * v28_9_0 + WQz * v28_9_1 + (VT)2.0 * oo2ze * v15_9_1 + (VT)2.0 * oo2e * (v28_3_0 - rho_e * v28_3_1);
-            const VT v29_19_0 = QCz * v29_9_0 + WQz * v29_9_1 + (VT)3.0 * oo2ze * v14_9_1 + (VT)2.0 * oo2e * (v29_3_0 - rho_e * v29_3_1);
-            const VT v30_19_0 = QCz * v30_9_0 + WQz * v30_9_1 + (VT)2.0 * oo2e * (v30_3_0 - rho_e * v30_3_1);
-            const VT v31_19_0 = QCz * v31_9_0 + WQz * v31_9_1 + (VT)1.0 * oo2ze * v16_9_1 + (VT)2.0 * oo2e * (v31_3_0 - rho_e * v31_3_1);
-            const VT v32_19_0 = QCz * v32_9_0 + WQz * v32_9_1 + (VT)2.0 * oo2ze * v17_9_1 + (VT)2.0 * oo2e * (v32_3_0 - rho_e * v32_3_1);
-            const VT v33_19_0 = QCz * v33_9_0 + WQz * v33_9_1 + (VT)3.0 * oo2ze * v18_9_1 + (VT)2.0 * oo2e * (v33_3_0 - rho_e * v33_3_1);
-            const VT v34_19_0 = QCz * v34_9_0 + WQz * v34_9_1 + (VT)4.0 * oo2ze * v19_9_1 + (VT)2.0 * oo2e * (v34_3_0 - rho_e * v34_3_1);
-            acc[0] += (double)v4_4_0;
-            acc[1] += (double)v4_5_0;
-            acc[2] += (double)v4_6_0;
-            acc[3] += (double)v4_7_0;
-            acc[4] += (double)v4_8_0;
-            acc[5] += (double)v4_9_0;
-            acc[6] += (double)v4_10_0;
-            acc[7] += (double)v4_11_0;
-            acc[8] += (double)v4_12_0;
-            acc[9] += (double)v4_13_0;
-            acc[10] += (double)v4_14_0;
-            acc[11] += (double)v4_15_0;
-            acc[12] += (double)v4_16_0;
-            acc[13] += (double)v4_17_0;
-            acc[14] += (double)v4_18_0;
-            acc[15] += (double)v4_19_0;
-            acc[16] += (double)v5_4_0;
-            acc[17] += (double)v5_5_0;
-            acc[18] += (double)v5_6_0;
-            acc[19] += (double)v5_7_0;
-            acc[20] += (double)v5_8_0;
-            acc[21] += (double)v5_9_0;
-            acc[22] += (double)v5_10_0;
-            acc[23] += (double)v5_11_0;
-            acc[24] += (double)v5_12_0;
-            acc[25] += (double)v5_13_0;
-            acc[26] += (double)v5_14_0;
-            acc[27] += (double)v5_15_0;
-            acc[28] += (double)v5_16_0;
-            acc[29] += (double)v5_17_0;
-            acc[30] += (double)v5_18_0;
-            acc[31] += (double)v5_19_0;
-            acc[32] += (double)v6_4_0;
-            acc[33] += (double)v6_5_0;
-            acc[34] += (double)v6_6_0;
-            acc[35] += (double)v6_7_0;
-            acc[36] += (double)v6_8_0;
-            acc[37] += (double)v6_9_0;
-            acc[38] += (double)v6_10_0;
-            acc[39] += (double)v6_11_0;
-            acc[40] += (double)v6_12_0;
-            acc[41] += (double)v6_13_0;
-            acc[42] += (double)v6_14_0;
-            acc[43] += (double)v6_15_0;
-            acc[44] += (double)v6_16_0;
-            acc[45] += (double)v6_17_0;
-            acc[46] += (double)v6_18_0;
-            acc[47] += (double)v6_19_0;
-            acc[48] += (double)v7_4_0;
-            acc[49] += (double)v7_5_0;
-            acc[50] += (double)v7_6_0;
-            acc[51] += (double)v7_7_0;
-            acc[52] += (double)v7_8_0;
-            acc[53] += (double)v7_9_0;
-            acc[54] += (double)v7_10_0;
-            acc[55] += (double)v7_11_0;
-            acc[56] += (double)v7_12_0;
-            acc[57] += (double)v7_13_0;
-            acc[58] += (double)v7_14_0;
-            acc[59] += (double)v7_15_0;
-            acc[60] += (double)v7_16_0;
-            acc[61] += (double)v7_17_0;
-            acc[62] += (double)v7_18_0;
-            acc[63] += (double)v7_19_0;
-            acc[64] += (double)v8_4_0;
-            acc[65] += (double)v8_5_0;
-            acc[66] += (double)v8_6_0;
-            acc[67] += (double)v8_7_0;
-            acc[68] += (double)v8_8_0;
-            acc[69] += (double)v8_9_0;
-            acc[70] += (double)v8_10_0;
-            acc[71] += (double)v8_11_0;
-            acc[72] += (double)v8_12_0;
-            acc[73] += (double)v8_13_0;
-            acc[74] += (double)v8_14_0;
-            acc[75] += (double)v8_15_0;
-            acc[76] += (double)v8_16_0;
-            acc[77] += (double)v8_17_0;
-            acc[78] += (double)v8_18_0;
-            acc[79] += (double)v8_19_0;
-            acc[80] += (double)v9_4_0;
-            acc[81] += (double)v9_5_0;
-            acc[82] += (double)v9_6_0;
-            acc[83] += (double)v9_7_0;
-            acc[84] += (double)v9_8_0;
-            acc[85] += (double)v9_9_0;
-            acc[86] += (double)v9_10_0;
-            acc[87] += (double)v9_11_0;
-            acc[88] += (double)v9_12_0;
-            acc[89] += (double)v9_13_0;
-            acc[90] += (double)v9_14_0;
-            acc[91] += (double)v9_15_0;
-            acc[92] += (double)v9_16_0;
-            acc[93] += (double)v9_17_0;
-            acc[94] += (double)v9_18_0;
-            acc[95] += (double)v9_19_0;
-            acc[96] += (double)v10_4_0;
-            acc[97] += (double)v10_5_0;
-            acc[98] += (double)v10_6_0;
-            acc[99] += (double)v10_7_0;
-            acc[100] += (double)v10_8_0;
-            acc[101] += (double)v10_9_0;
-            acc[102] += (double)v10_10_0;
-            acc[103] += (double)v10_11_0;
-            acc[104] += (double)v10_12_0;
-            acc[105] += (double)v10_13_0;
-            acc[106] += (double)v10_14_0;
-            acc[107] += (double)v10_15_0;
-            acc[108] += (double)v10_16_0;
-            acc[109] += (double)v10_17_0;
-            acc[110] += (double)v10_18_0;
-            acc[111] += (double)v10_19_0;
-            acc[112] += (double)v11_4_0;
-            acc[113] += (double)v11_5_0;
-            acc[114] += (double)v11_6_0;
-            acc[115] += (double)v11_7_0;
-            acc[116] += (double)v11_8_0;
-            acc[117] += (double)v11_9_0;
-            acc[118] += (double)v11_10_0;
-            acc[119] += (double)v11_11_0;
-            acc[120] += (double)v11_12_0;
-            acc[121] += (double)v11_13_0;
-            acc[122] += (double)v11_14_0;
-            acc[123] += (double)v11_15_0;
-            acc[124] += (double)v11_16_0;
-            acc[125] += (double)v11_17_0;
-            acc[126] += (double)v11_18_0;
-            acc[127] += (double)v11_19_0;
-            acc[128] += (double)v12_4_0;
-            acc[129] += (double)v12_5_0;
-            acc[130] += (double)v12_6_0;
-            acc[131] += (double)v12_7_0;
-            acc[132] += (double)v12_8_0;
-            acc[133] += (double)v12_9_0;
-            acc[134] += (double)v12_10_0;
-            acc[135] += (double)v12_11_0;
-            acc[136] += (double)v12_12_0;
-            acc[137] += (double)v12_13_0;
-            acc[138] += (double)v12_14_0;
-            acc[139] += (double)v12_15_0;
-            acc[140] += (double)v12_16_0;
-            acc[141] += (double)v12_17_0;
-            acc[142] += (double)v12_18_0;
-            acc[143] += (double)v12_19_0;
-            acc[144] += (double)v13_4_0;
-            acc[145] += (double)v13_5_0;
-            acc[146] += (double)v13_6_0;
-            acc[147] += (double)v13_7_0;
-            acc[148] += (double)v13_8_0;
-            acc[149] += (double)v13_9_0;
-            acc[150] += (double)v13_10_0;
-            acc[151] += (double)v13_11_0;
-            acc[152] += (double)v13_12_0;
-            acc[153] += (double)v13_13_0;
-            acc[154] += (double)v13_14_0;
-            acc[155] += (double)v13_15_0;
-            acc[156] += (double)v13_16_0;
-            acc[157] += (double)v13_17_0;
-            acc[158] += (double)v13_18_0;
-            acc[159] += (double)v13_19_0;
-            acc[160] += (double)v14_4_0;
-            acc[161] += (double)v14_5_0;
-            acc[162] += (double)v14_6_0;
-            acc[163] += (double)v14_7_0;
-            acc[164] += (double)v14_8_0;
-            acc[165] += (double)v14_9_0;
-            acc[166] += (double)v14_10_0;
-            acc[167] += (double)v14_11_0;
-            acc[168] += (double)v14_12_0;
-            acc[169] += (double)v14_13_0;
-            acc[170] += (double)v14_14_0;
-            acc[171] += (double)v14_15_0;
-            acc[172] += (double)v14_16_0;
-            acc[173] += (double)v14_17_0;
-            acc[174] += (double)v14_18_0;
-            acc[175] += (double)v14_19_0;
-            acc[176] += (double)v15_4_0;
-            acc[177] += (double)v15_5_0;
-            acc[178] += (double)v15_6_0;
-            acc[179] += (double)v15_7_0;
-            acc[180] += (double)v15_8_0;
-            acc[181] += (double)v15_9_0;
-            acc[182] += (double)v15_10_0;
-            acc[183] += (double)v15_11_0;
-            acc[184] += (double)v15_12_0;
-            acc[185] += (double)v15_13_0;
-            acc[186] += (double)v15_14_0;
-            acc[187] += (double)v15_15_0;
-            acc[188] += (double)v15_16_0;
-            acc[189] += (double)v15_17_0;
-            acc[190] += (double)v15_18_0;
-            acc[191] += (double)v15_19_0;
-            acc[192] += (double)v16_4_0;
-            acc[193] += (double)v16_5_0;
-            acc[194] += (double)v16_6_0;
-            acc[195] += (double)v16_7_0;
-            acc[196] += (double)v16_8_0;
-            acc[197] += (double)v16_9_0;
-            acc[198] += (double)v16_10_0;
-            acc[199] += (double)v16_11_0;
-            acc[200] += (double)v16_12_0;
-            acc[201] += (double)v16_13_0;
-            acc[202] += (double)v16_14_0;
-            acc[203] += (double)v16_15_0;
-            acc[204] += (double)v16_16_0;
-            acc[205] += (double)v16_17_0;
-            acc[206] += (double)v16_18_0;
-            acc[207] += (double)v16_19_0;
-            acc[208] += (double)v17_4_0;
-            acc[209] += (double)v17_5_0;
-            acc[210] += (double)v17_6_0;
-            acc[211] += (double)v17_7_0;
-            acc[212] += (double)v17_8_0;
-            acc[213] += (double)v17_9_0;
-            acc[214] += (double)v17_10_0;
-            acc[215] += (double)v17_11_0;
-            acc[216] += (double)v17_12_0;
-            acc[217] += (double)v17_13_0;
-            acc[218] += (double)v17_14_0;
-            acc[219] += (double)v17_15_0;
-            acc[220] += (double)v17_16_0;
-            acc[221] += (double)v17_17_0;
-            acc[222] += (double)v17_18_0;
-            acc[223] += (double)v17_19_0;
-            acc[224] += (double)v18_4_0;
-            acc[225] += (double)v18_5_0;
-            acc[226] += (double)v18_6_0;
-            acc[227] += (double)v18_7_0;
-            acc[228] += (double)v18_8_0;
-            acc[229] += (double)v18_9_0;
-            acc[230] += (double)v18_10_0;
-            acc[231] += (double)v18_11_0;
-            acc[232] += (double)v18_12_0;
-            acc[233] += (double)v18_13_0;
-            acc[234] += (double)v18_14_0;
-            acc[235] += (double)v18_15_0;
-            acc[236] += (double)v18_16_0;
-            acc[237] += (double)v18_17_0;
-            acc[238] += (double)v18_18_0;
-            acc[239] += (double)v18_19_0;
-            acc[240] += (double)v19_4_0;
-            acc[241] += (double)v19_5_0;
-            acc[242] += (double)v19_6_0;
-            acc[243] += (double)v19_7_0;
-            acc[244] += (double)v19_8_0;
-            acc[245] += (double)v19_9_0;
-            acc[246] += (double)v19_10_0;
-            acc[247] += (double)v19_11_0;
-            acc[248] += (double)v19_12_0;
-            acc[249] += (double)v19_13_0;
-            acc[250] += (double)v19_14_0;
-            acc[251] += (double)v19_15_0;
-            acc[252] += (double)v19_16_0;
-            acc[253] += (double)v19_17_0;
-            acc[254] += (double)v19_18_0;
-            acc[255] += (double)v19_19_0;
-            acc[256] += (double)v20_4_0;
-            acc[257] += (double)v20_5_0;
-            acc[258] += (double)v20_6_0;
-            acc[259] += (double)v20_7_0;
-            acc[260] += (double)v20_8_0;
-            acc[261] += (double)v20_9_0;
-            acc[262] += (double)v20_10_0;
-            acc[263] += (double)v20_11_0;
-            acc[264] += (double)v20_12_0;
-            acc[265] += (double)v20_13_0;
-            acc[266] += (double)v20_14_0;
-            acc[267] += (double)v20_15_0;
-            acc[268] += (double)v20_16_0;
-            acc[269] += (double)v20_17_0;
-            acc[270] += (double)v20_18_0;
-            acc[271] += (double)v20_19_0;
-            acc[272] += (double)v21_4_0;
-            acc[273] += (double)v21_5_0;
-            acc[274] += (double)v21_6_0;
-            acc[275] += (double)v21_7_0;
-            acc[276] += (double)v21_8_0;
-            acc[277] += (double)v21_9_0;
-            acc[278] += (double)v21_10_0;
-            acc[279] += (double)v21_11_0;
-            acc[280] += (double)v21_12_0;
-            acc[281] += (double)v21_13_0;
-            acc[282] += (double)v21_14_0;
-            acc[283] += (double)v21_15_0;
-            acc[284] += (double)v21_16_0;
-            acc[285] += (double)v21_17_0;
-            acc[286] += (double)v21_18_0;
-            acc[287] += (double)v21_19_0;
-            acc[288] += (double)v22_4_0;
-            acc[289] += (double)v22_5_0;
-            acc[290] += (double)v22_6_0;
-            acc[291] += (double)v22_7_0;
-            acc[292] += (double)v22_8_0;
-            acc[293] += (double)v22_9_0;
-            acc[294] += (double)v22_10_0;
-            acc[295] += (double)v22_11_0;
-            acc[296] += (double)v22_12_0;
-            acc[297] += (double)v22_13_0;
-            acc[298] += (double)v22_14_0;
-            acc[299] += (double)v22_15_0;
-            acc[300] += (double)v22_16_0;
-            acc[301] += (double)v22_17_0;
-            acc[302] += (double)v22_18_0;
-            acc[303] += (double)v22_19_0;
-            acc[304] += (double)v23_4_0;
-            acc[305] += (double)v23_5_0;
-            acc[306] += (double)v23_6_0;
-            acc[307] += (double)v23_7_0;
-            acc[308] += (double)v23_8_0;
-            acc[309] += (double)v23_9_0;
-            acc[310] += (double)v23_10_0;
-            acc[311] += (double)v23_11_0;
-            acc[312] += (double)v23_12_0;
-            acc[313] += (double)v23_13_0;
-            acc[314] += (double)v23_14_0;
-            acc[315] += (double)v23_15_0;
-            acc[316] += (double)v23_16_0;
-            acc[317] += (double)v23_17_0;
-            acc[318] += (double)v23_18_0;
-            acc[319] += (double)v23_19_0;
-            acc[320] += (double)v24_4_0;
-            acc[321] += (double)v24_5_0;
-            acc[322] += (double)v24_6_0;
-            acc[323] += (double)v24_7_0;
-            acc[324] += (double)v24_8_0;
-            acc[325] += (double)v24_9_0;
-            acc[326] += (double)v24_10_0;
-            acc[327] += (double)v24_11_0;
-            acc[328] += (double)v24_12_0;
-            acc[329] += (double)v24_13_0;
-            acc[330] += (double)v24_14_0;
-            acc[331] += (double)v24_15_0;
-            acc[332] += (double)v24_16_0;
-            acc[333] += (double)v24_17_0;
-            acc[334] += (double)v24_18_0;
-            acc[335] += (double)v24_19_0;
-            acc[336] += (double)v25_4_0;
-            acc[337] += (double)v25_5_0;
-            acc[338] += (double)v25_6_0;
-            acc[339] += (double)v25_7_0;
-            acc[340] += (double)v25_8_0;
-            acc[341] += (double)v25_9_0;
-            acc[342] += (double)v25_10_0;
-            acc[343] += (double)v25_11_0;
-            acc[344] += (double)v25_12_0;
-            acc[345] += (double)v25_13_0;
-            acc[346] += (double)v25_14_0;
-            acc[347] += (double)v25_15_0;
-            acc[348] += (double)v25_16_0;
-            acc[349] += (double)v25_17_0;
-            acc[350] += (double)v25_18_0;
-            acc[351] += (double)v25_19_0;
-            acc[352] += (double)v26_4_0;
-            acc[353] += (double)v26_5_0;
-            acc[354] += (double)v26_6_0;
-            acc[355] += (double)v26_7_0;
-            acc[356] += (double)v26_8_0;
-            acc[357] += (double)v26_9_0;
-            acc[358] += (double)v26_10_0;
-            acc[359] += (double)v26_11_0;
-            acc[360] += (double)v26_12_0;
-            acc[361] += (double)v26_13_0;
-            acc[362] += (double)v26_14_0;
-            acc[363] += (double)v26_15_0;
-            acc[364] += (double)v26_16_0;
-            acc[365] += (double)v26_17_0;
-            acc[366] += (double)v26_18_0;
-            acc[367] += (double)v26_19_0;
-            acc[368] += (double)v27_4_0;
-            acc[369] += (double)v27_5_0;
-            acc[370] += (double)v27_6_0;
-            acc[371] += (double)v27_7_0;
-            acc[372] += (double)v27_8_0;
-            acc[373] += (double)v27_9_0;
-            acc[374] += (double)v27_10_0;
-            acc[375] += (double)v27_11_0;
-            acc[376] += (double)v27_12_0;
-            acc[377] += (double)v27_13_0;
-            acc[378] += (double)v27_14_0;
-            acc[379] += (double)v27_15_0;
-            acc[380] += (double)v27_16_0;
-            acc[381] += (double)v27_17_0;
-            acc[382] += (double)v27_18_0;
-            acc[383] += (double)v27_19_0;
-            acc[384] += (double)v28_4_0;
-            acc[385] += (double)v28_5_0;
-            acc[386] += (double)v28_6_0;
-            acc[387] += (double)v28_7_0;
-            acc[388] += (double)v28_8_0;
-            acc[389] += (double)v28_9_0;
-            acc[390] += (double)v28_10_0;
-            acc[391] += (double)v28_11_0;
-            acc[392] += (double)v28_12_0;
-            acc[393] += (double)v28_13_0;
-            acc[394] += (double)v28_14_0;
-            acc[395] += (double)v28_15_0;
-            acc[396] += (double)v28_16_0;
-            acc[397] += (double)v28_17_0;
-            acc[398] += (double)v28_18_0;
-            acc[399] += (double)v28_19_0;
-            acc[400] += (double)v29_4_0;
-            acc[401] += (double)v29_5_0;
-            acc[402] += (double)v29_6_0;
-            acc[403] += (double)v29_7_0;
-            acc[404] += (double)v29_8_0;
-            acc[405] += (double)v29_9_0;
-            acc[406] += (double)v29_10_0;
-            acc[407] += (double)v29_11_0;
-            acc[408] += (double)v29_12_0;
-            acc[409] += (double)v29_13_0;
-            acc[410] += (double)v29_14_0;
-            acc[411] += (double)v29_15_0;
-            acc[412] += (double)v29_16_0;
-            acc[413] += (double)v29_17_0;
-            acc[414] += (double)v29_18_0;
-            acc[415] += (double)v29_19_0;
-            acc[416] += (double)v30_4_0;
-            acc[417] += (double)v30_5_0;
-            acc[418] += (double)v30_6_0;
-            acc[419] += (double)v30_7_0;
-            acc[420] += (double)v30_8_0;
-            acc[421] += (double)v30_9_0;
-            acc[422] += (double)v30_10_0;
-            acc[423] += (double)v30_11_0;
-            acc[424] += (double)v30_12_0;
-            acc[425] += (double)v30_13_0;
-            acc[426] += (double)v30_14_0;
-            acc[427] += (double)v30_15_0;
-            acc[428] += (double)v30_16_0;
-            acc[429] += (double)v30_17_0;
-            acc[430] += (double)v30_18_0;
-            acc[431] += (double)v30_19_0;
-            acc[432] += (double)v31_4_0;
-            acc[433] += (double)v31_5_0;
-            acc[434] += (double)v31_6_0;
-            acc[435] += (double)v31_7_0;
-            acc[436] += (double)v31_8_0;
-            acc[437] += (double)v31_9_0;
-            acc[438] += (double)v31_10_0;
-            acc[439] += (double)v31_11_0;
-            acc[440] += (double)v31_12_0;
-            acc[441] += (double)v31_13_0;
-            acc[442] += (double)v31_14_0;
-            acc[443] += (double)v31_15_0;
-            acc[444] += (double)v31_16_0;
-            acc[445] += (double)v31_17_0;
-            acc[446] += (double)v31_18_0;
-            acc[447] += (double)v31_19_0;
-            acc[448] += (double)v32_4_0;
-            acc[449] += (double)v32_5_0;
-            acc[450] += (double)v32_6_0;
-            acc[451] += (double)v32_7_0;
-            acc[452] += (double)v32_8_0;
-            acc[453] += (double)v32_9_0;
-            acc[454] += (double)v32_10_0;
-            acc[455] += (double)v32_11_0;
-            acc[456] += (double)v32_12_0;
-            acc[457] += (double)v32_13_0;
-            acc[458] += (double)v32_14_0;
-            acc[459] += (double)v32_15_0;
-            acc[460] += (double)v32_16_0;
-            acc[461] += (double)v32_17_0;
-            acc[462] += (double)v32_18_0;
-            acc[463] += (double)v32_19_0;
-            acc[464] += (double)v33_4_0;
-            acc[465] += (double)v33_5_0;
-            acc[466] += (double)v33_6_0;
-            acc[467] += (double)v33_7_0;
-            acc[468] += (double)v33_8_0;
-            acc[469] += (double)v33_9_0;
-            acc[470] += (double)v33_10_0;
-            acc[471] += (double)v33_11_0;
-            acc[472] += (double)v33_12_0;
-            acc[473] += (double)v33_13_0;
-            acc[474] += (double)v33_14_0;
-            acc[475] += (double)v33_15_0;
-            acc[476] += (double)v33_16_0;
-            acc[477] += (double)v33_17_0;
-            acc[478] += (double)v33_18_0;
-            acc[479] += (double)v33_19_0;
-            acc[480] += (double)v34_4_0;
-            acc[481] += (double)v34_5_0;
-            acc[482] += (double)v34_6_0;
-            acc[483] += (double)v34_7_0;
-            acc[484] += (double)v34_8_0;
-            acc[485] += (double)v34_9_0;
-            acc[486] += (double)v34_10_0;
-            acc[487] += (double)v34_11_0;
-            acc[488] += (double)v34_12_0;
-            acc[489] += (double)v34_13_0;
-            acc[490] += (double)v34_14_0;
-            acc[491] += (double)v34_15_0;
-            acc[492] += (double)v34_16_0;
-            acc[493] += (double)v34_17_0;
-            acc[494] += (double)v34_18_0;
-            acc[495] += (double)v34_19_0;
+            if constexpr (sizeof(VT) == 8) {
+                acc[0] += (double)v4_4_0;
+                acc[1] += (double)v4_5_0;
+                acc[2] += (double)v4_6_0;
+                acc[3] += (double)v4_7_0;
+                acc[4] += (double)v4_8_0;
+                acc[5] += (double)v4_9_0;
+                acc[6] = fma(QCx, v4_4_0, fma(WQx, v4_4_1, fma(2.0 * oo2ze, v1_4_1, fma(2.0 * oo2e, (v4_1_0 - rho_e * v4_1_1), acc[6]))));
+                acc[7] = fma(QCx, v4_5_0, fma(WQx, v4_5_1, fma(2.0 * oo2ze, v1_5_1, fma(1.0 * oo2e, (v4_2_0 - rho_e * v4_2_1), acc[7]))));
+                acc[8] = fma(QCx, v4_6_0, fma(WQx, v4_6_1, fma(2.0 * oo2ze, v1_6_1, fma(1.0 * oo2e, (v4_3_0 - rho_e * v4_3_1), acc[8]))));
+                acc[9] = fma(QCy, v4_5_0, fma(WQy, v4_5_1, fma(1.0 * oo2e, (v4_1_0 - rho_e * v4_1_1), acc[9])));
+                acc[10] = fma(QCz, v4_6_0, fma(WQz, v4_6_1, fma(1.0 * oo2e, (v4_1_0 - rho_e * v4_1_1), acc[10])));
+                acc[11] = fma(QCx, v4_8_0, fma(WQx, v4_8_1, fma(2.0 * oo2ze, v1_8_1, acc[11])));
+                acc[12] = fma(QCy, v4_7_0, fma(WQy, v4_7_1, fma(2.0 * oo2e, (v4_2_0 - rho_e * v4_2_1), acc[12])));
+                acc[13] = fma(QCy, v4_8_0, fma(WQy, v4_8_1, fma(1.0 * oo2e, (v4_3_0 - rho_e * v4_3_1), acc[13])));
+                acc[14] = fma(QCz, v4_8_0, fma(WQz, v4_8_1, fma(1.0 * oo2e, (v4_2_0 - rho_e * v4_2_1), acc[14])));
+                acc[15] = fma(QCz, v4_9_0, fma(WQz, v4_9_1, fma(2.0 * oo2e, (v4_3_0 - rho_e * v4_3_1), acc[15])));
+                acc[16] += (double)v5_4_0;
+                acc[17] += (double)v5_5_0;
+                acc[18] += (double)v5_6_0;
+                acc[19] += (double)v5_7_0;
+                acc[20] += (double)v5_8_0;
+                acc[21] += (double)v5_9_0;
+                acc[22] = fma(QCx, v5_4_0, fma(WQx, v5_4_1, fma(1.0 * oo2ze, v2_4_1, fma(2.0 * oo2e, (v5_1_0 - rho_e * v5_1_1), acc[22]))));
+                acc[23] = fma(QCx, v5_5_0, fma(WQx, v5_5_1, fma(1.0 * oo2ze, v2_5_1, fma(1.0 * oo2e, (v5_2_0 - rho_e * v5_2_1), acc[23]))));
+                acc[24] = fma(QCx, v5_6_0, fma(WQx, v5_6_1, fma(1.0 * oo2ze, v2_6_1, fma(1.0 * oo2e, (v5_3_0 - rho_e * v5_3_1), acc[24]))));
+                acc[25] = fma(QCy, v5_5_0, fma(WQy, v5_5_1, fma(1.0 * oo2ze, v1_5_1, fma(1.0 * oo2e, (v5_1_0 - rho_e * v5_1_1), acc[25]))));
+                acc[26] = fma(QCz, v5_6_0, fma(WQz, v5_6_1, fma(1.0 * oo2e, (v5_1_0 - rho_e * v5_1_1), acc[26])));
+                acc[27] = fma(QCx, v5_8_0, fma(WQx, v5_8_1, fma(1.0 * oo2ze, v2_8_1, acc[27])));
+                acc[28] = fma(QCy, v5_7_0, fma(WQy, v5_7_1, fma(1.0 * oo2ze, v1_7_1, fma(2.0 * oo2e, (v5_2_0 - rho_e * v5_2_1), acc[28]))));
+                acc[29] = fma(QCy, v5_8_0, fma(WQy, v5_8_1, fma(1.0 * oo2ze, v1_8_1, fma(1.0 * oo2e, (v5_3_0 - rho_e * v5_3_1), acc[29]))));
+                acc[30] = fma(QCz, v5_8_0, fma(WQz, v5_8_1, fma(1.0 * oo2e, (v5_2_0 - rho_e * v5_2_1), acc[30])));
+                acc[31] = fma(QCz, v5_9_0, fma(WQz, v5_9_1, fma(2.0 * oo2e, (v5_3_0 - rho_e * v5_3_1), acc[31])));
+                acc[32] += (double)v6_4_0;
+                acc[33] += (double)v6_5_0;
+                acc[34] += (double)v6_6_0;
+                acc[35] += (double)v6_7_0;
+                acc[36] += (double)v6_8_0;
+                acc[37] += (double)v6_9_0;
+                acc[38] = fma(QCx, v6_4_0, fma(WQx, v6_4_1, fma(1.0 * oo2ze, v3_4_1, fma(2.0 * oo2e, (v6_1_0 - rho_e * v6_1_1), acc[38]))));
+                acc[39] = fma(QCx, v6_5_0, fma(WQx, v6_5_1, fma(1.0 * oo2ze, v3_5_1, fma(1.0 * oo2e, (v6_2_0 - rho_e * v6_2_1), acc[39]))));
+                acc[40] = fma(QCx, v6_6_0, fma(WQx, v6_6_1, fma(1.0 * oo2ze, v3_6_1, fma(1.0 * oo2e, (v6_3_0 - rho_e * v6_3_1), acc[40]))));
+                acc[41] = fma(QCy, v6_5_0, fma(WQy, v6_5_1, fma(1.0 * oo2e, (v6_1_0 - rho_e * v6_1_1), acc[41])));
+                acc[42] = fma(QCz, v6_6_0, fma(WQz, v6_6_1, fma(1.0 * oo2ze, v1_6_1, fma(1.0 * oo2e, (v6_1_0 - rho_e * v6_1_1), acc[42]))));
+                acc[43] = fma(QCx, v6_8_0, fma(WQx, v6_8_1, fma(1.0 * oo2ze, v3_8_1, acc[43])));
+                acc[44] = fma(QCy, v6_7_0, fma(WQy, v6_7_1, fma(2.0 * oo2e, (v6_2_0 - rho_e * v6_2_1), acc[44])));
+                acc[45] = fma(QCy, v6_8_0, fma(WQy, v6_8_1, fma(1.0 * oo2e, (v6_3_0 - rho_e * v6_3_1), acc[45])));
+                acc[46] = fma(QCz, v6_8_0, fma(WQz, v6_8_1, fma(1.0 * oo2ze, v1_8_1, fma(1.0 * oo2e, (v6_2_0 - rho_e * v6_2_1), acc[46]))));
+                acc[47] = fma(QCz, v6_9_0, fma(WQz, v6_9_1, fma(1.0 * oo2ze, v1_9_1, fma(2.0 * oo2e, (v6_3_0 - rho_e * v6_3_1), acc[47]))));
+                acc[48] += (double)v7_4_0;
+                acc[49] += (double)v7_5_0;
+                acc[50] += (double)v7_6_0;
+                acc[51] += (double)v7_7_0;
+                acc[52] += (double)v7_8_0;
+                acc[53] += (double)v7_9_0;
+                acc[54] = fma(QCx, v7_4_0, fma(WQx, v7_4_1, fma(2.0 * oo2e, (v7_1_0 - rho_e * v7_1_1), acc[54])));
+                acc[55] = fma(QCx, v7_5_0, fma(WQx, v7_5_1, fma(1.0 * oo2e, (v7_2_0 - rho_e * v7_2_1), acc[55])));
+                acc[56] = fma(QCx, v7_6_0, fma(WQx, v7_6_1, fma(1.0 * oo2e, (v7_3_0 - rho_e * v7_3_1), acc[56])));
+                acc[57] = fma(QCy, v7_5_0, fma(WQy, v7_5_1, fma(2.0 * oo2ze, v2_5_1, fma(1.0 * oo2e, (v7_1_0 - rho_e * v7_1_1), acc[57]))));
+                acc[58] = fma(QCz, v7_6_0, fma(WQz, v7_6_1, fma(1.0 * oo2e, (v7_1_0 - rho_e * v7_1_1), acc[58])));
+                acc[59] = fma(QCx, v7_8_0, fma(WQx, v7_8_1, acc[59]));
+                acc[60] = fma(QCy, v7_7_0, fma(WQy, v7_7_1, fma(2.0 * oo2ze, v2_7_1, fma(2.0 * oo2e, (v7_2_0 - rho_e * v7_2_1), acc[60]))));
+                acc[61] = fma(QCy, v7_8_0, fma(WQy, v7_8_1, fma(2.0 * oo2ze, v2_8_1, fma(1.0 * oo2e, (v7_3_0 - rho_e * v7_3_1), acc[61]))));
+                acc[62] = fma(QCz, v7_8_0, fma(WQz, v7_8_1, fma(1.0 * oo2e, (v7_2_0 - rho_e * v7_2_1), acc[62])));
+                acc[63] = fma(QCz, v7_9_0, fma(WQz, v7_9_1, fma(2.0 * oo2e, (v7_3_0 - rho_e * v7_3_1), acc[63])));
+                acc[64] += (double)v8_4_0;
+                acc[65] += (double)v8_5_0;
+                acc[66] += (double)v8_6_0;
+                acc[67] += (double)v8_7_0;
+                acc[68] += (double)v8_8_0;
+                acc[69] += (double)v8_9_0;
+                acc[70] = fma(QCx, v8_4_0, fma(WQx, v8_4_1, fma(2.0 * oo2e, (v8_1_0 - rho_e * v8_1_1), acc[70])));
+                acc[71] = fma(QCx, v8_5_0, fma(WQx, v8_5_1, fma(1.0 * oo2e, (v8_2_0 - rho_e * v8_2_1), acc[71])));
+                acc[72] = fma(QCx, v8_6_0, fma(WQx, v8_6_1, fma(1.0 * oo2e, (v8_3_0 - rho_e * v8_3_1), acc[72])));
+                acc[73] = fma(QCy, v8_5_0, fma(WQy, v8_5_1, fma(1.0 * oo2ze, v3_5_1, fma(1.0 * oo2e, (v8_1_0 - rho_e * v8_1_1), acc[73]))));
+                acc[74] = fma(QCz, v8_6_0, fma(WQz, v8_6_1, fma(1.0 * oo2ze, v2_6_1, fma(1.0 * oo2e, (v8_1_0 - rho_e * v8_1_1), acc[74]))));
+                acc[75] = fma(QCx, v8_8_0, fma(WQx, v8_8_1, acc[75]));
+                acc[76] = fma(QCy, v8_7_0, fma(WQy, v8_7_1, fma(1.0 * oo2ze, v3_7_1, fma(2.0 * oo2e, (v8_2_0 - rho_e * v8_2_1), acc[76]))));
+                acc[77] = fma(QCy, v8_8_0, fma(WQy, v8_8_1, fma(1.0 * oo2ze, v3_8_1, fma(1.0 * oo2e, (v8_3_0 - rho_e * v8_3_1), acc[77]))));
+                acc[78] = fma(QCz, v8_8_0, fma(WQz, v8_8_1, fma(1.0 * oo2ze, v2_8_1, fma(1.0 * oo2e, (v8_2_0 - rho_e * v8_2_1), acc[78]))));
+                acc[79] = fma(QCz, v8_9_0, fma(WQz, v8_9_1, fma(1.0 * oo2ze, v2_9_1, fma(2.0 * oo2e, (v8_3_0 - rho_e * v8_3_1), acc[79]))));
+                acc[80] += (double)v9_4_0;
+                acc[81] += (double)v9_5_0;
+                acc[82] += (double)v9_6_0;
+                acc[83] += (double)v9_7_0;
+                acc[84] += (double)v9_8_0;
+                acc[85] += (double)v9_9_0;
+                acc[86] = fma(QCx, v9_4_0, fma(WQx, v9_4_1, fma(2.0 * oo2e, (v9_1_0 - rho_e * v9_1_1), acc[86])));
+                acc[87] = fma(QCx, v9_5_0, fma(WQx, v9_5_1, fma(1.0 * oo2e, (v9_2_0 - rho_e * v9_2_1), acc[87])));
+                acc[88] = fma(QCx, v9_6_0, fma(WQx, v9_6_1, fma(1.0 * oo2e, (v9_3_0 - rho_e * v9_3_1), acc[88])));
+                acc[89] = fma(QCy, v9_5_0, fma(WQy, v9_5_1, fma(1.0 * oo2e, (v9_1_0 - rho_e * v9_1_1), acc[89])));
+                acc[90] = fma(QCz, v9_6_0, fma(WQz, v9_6_1, fma(2.0 * oo2ze, v3_6_1, fma(1.0 * oo2e, (v9_1_0 - rho_e * v9_1_1), acc[90]))));
+                acc[91] = fma(QCx, v9_8_0, fma(WQx, v9_8_1, acc[91]));
+                acc[92] = fma(QCy, v9_7_0, fma(WQy, v9_7_1, fma(2.0 * oo2e, (v9_2_0 - rho_e * v9_2_1), acc[92])));
+                acc[93] = fma(QCy, v9_8_0, fma(WQy, v9_8_1, fma(1.0 * oo2e, (v9_3_0 - rho_e * v9_3_1), acc[93])));
+                acc[94] = fma(QCz, v9_8_0, fma(WQz, v9_8_1, fma(2.0 * oo2ze, v3_8_1, fma(1.0 * oo2e, (v9_2_0 - rho_e * v9_2_1), acc[94]))));
+                acc[95] = fma(QCz, v9_9_0, fma(WQz, v9_9_1, fma(2.0 * oo2ze, v3_9_1, fma(2.0 * oo2e, (v9_3_0 - rho_e * v9_3_1), acc[95]))));
+                acc[96] += (double)v10_4_0;
+                acc[97] += (double)v10_5_0;
+                acc[98] += (double)v10_6_0;
+                acc[99] += (double)v10_7_0;
+                acc[100] += (double)v10_8_0;
+                acc[101] += (double)v10_9_0;
+                acc[102] = fma(QCx, v10_4_0, fma(WQx, v10_4_1, fma(3.0 * oo2ze, v4_4_1, fma(2.0 * oo2e, (v10_1_0 - rho_e * v10_1_1), acc[102]))));
+                acc[103] = fma(QCx, v10_5_0, fma(WQx, v10_5_1, fma(3.0 * oo2ze, v4_5_1, fma(1.0 * oo2e, (v10_2_0 - rho_e * v10_2_1), acc[103]))));
+                acc[104] = fma(QCx, v10_6_0, fma(WQx, v10_6_1, fma(3.0 * oo2ze, v4_6_1, fma(1.0 * oo2e, (v10_3_0 - rho_e * v10_3_1), acc[104]))));
+                acc[105] = fma(QCy, v10_5_0, fma(WQy, v10_5_1, fma(1.0 * oo2e, (v10_1_0 - rho_e * v10_1_1), acc[105])));
+                acc[106] = fma(QCz, v10_6_0, fma(WQz, v10_6_1, fma(1.0 * oo2e, (v10_1_0 - rho_e * v10_1_1), acc[106])));
+                acc[107] = fma(QCx, v10_8_0, fma(WQx, v10_8_1, fma(3.0 * oo2ze, v4_8_1, acc[107])));
+                acc[108] = fma(QCy, v10_7_0, fma(WQy, v10_7_1, fma(2.0 * oo2e, (v10_2_0 - rho_e * v10_2_1), acc[108])));
+                acc[109] = fma(QCy, v10_8_0, fma(WQy, v10_8_1, fma(1.0 * oo2e, (v10_3_0 - rho_e * v10_3_1), acc[109])));
+                acc[110] = fma(QCz, v10_8_0, fma(WQz, v10_8_1, fma(1.0 * oo2e, (v10_2_0 - rho_e * v10_2_1), acc[110])));
+                acc[111] = fma(QCz, v10_9_0, fma(WQz, v10_9_1, fma(2.0 * oo2e, (v10_3_0 - rho_e * v10_3_1), acc[111])));
+                acc[112] += (double)v11_4_0;
+                acc[113] += (double)v11_5_0;
+                acc[114] += (double)v11_6_0;
+                acc[115] += (double)v11_7_0;
+                acc[116] += (double)v11_8_0;
+                acc[117] += (double)v11_9_0;
+                acc[118] = fma(QCx, v11_4_0, fma(WQx, v11_4_1, fma(2.0 * oo2ze, v5_4_1, fma(2.0 * oo2e, (v11_1_0 - rho_e * v11_1_1), acc[118]))));
+                acc[119] = fma(QCx, v11_5_0, fma(WQx, v11_5_1, fma(2.0 * oo2ze, v5_5_1, fma(1.0 * oo2e, (v11_2_0 - rho_e * v11_2_1), acc[119]))));
+                acc[120] = fma(QCx, v11_6_0, fma(WQx, v11_6_1, fma(2.0 * oo2ze, v5_6_1, fma(1.0 * oo2e, (v11_3_0 - rho_e * v11_3_1), acc[120]))));
+                acc[121] = fma(QCy, v11_5_0, fma(WQy, v11_5_1, fma(1.0 * oo2ze, v4_5_1, fma(1.0 * oo2e, (v11_1_0 - rho_e * v11_1_1), acc[121]))));
+                acc[122] = fma(QCz, v11_6_0, fma(WQz, v11_6_1, fma(1.0 * oo2e, (v11_1_0 - rho_e * v11_1_1), acc[122])));
+                acc[123] = fma(QCx, v11_8_0, fma(WQx, v11_8_1, fma(2.0 * oo2ze, v5_8_1, acc[123])));
+                acc[124] = fma(QCy, v11_7_0, fma(WQy, v11_7_1, fma(1.0 * oo2ze, v4_7_1, fma(2.0 * oo2e, (v11_2_0 - rho_e * v11_2_1), acc[124]))));
+                acc[125] = fma(QCy, v11_8_0, fma(WQy, v11_8_1, fma(1.0 * oo2ze, v4_8_1, fma(1.0 * oo2e, (v11_3_0 - rho_e * v11_3_1), acc[125]))));
+                acc[126] = fma(QCz, v11_8_0, fma(WQz, v11_8_1, fma(1.0 * oo2e, (v11_2_0 - rho_e * v11_2_1), acc[126])));
+                acc[127] = fma(QCz, v11_9_0, fma(WQz, v11_9_1, fma(2.0 * oo2e, (v11_3_0 - rho_e * v11_3_1), acc[127])));
+                acc[128] += (double)v12_4_0;
+                acc[129] += (double)v12_5_0;
+                acc[130] += (double)v12_6_0;
+                acc[131] += (double)v12_7_0;
+                acc[132] += (double)v12_8_0;
+                acc[133] += (double)v12_9_0;
+                acc[134] = fma(QCx, v12_4_0, fma(WQx, v12_4_1, fma(2.0 * oo2ze, v6_4_1, fma(2.0 * oo2e, (v12_1_0 - rho_e * v12_1_1), acc[134]))));
+                acc[135] = fma(QCx, v12_5_0, fma(WQx, v12_5_1, fma(2.0 * oo2ze, v6_5_1, fma(1.0 * oo2e, (v12_2_0 - rho_e * v12_2_1), acc[135]))));
+                acc[136] = fma(QCx, v12_6_0, fma(WQx, v12_6_1, fma(2.0 * oo2ze, v6_6_1, fma(1.0 * oo2e, (v12_3_0 - rho_e * v12_3_1), acc[136]))));
+                acc[137] = fma(QCy, v12_5_0, fma(WQy, v12_5_1, fma(1.0 * oo2e, (v12_1_0 - rho_e * v12_1_1), acc[137])));
+                acc[138] = fma(QCz, v12_6_0, fma(WQz, v12_6_1, fma(1.0 * oo2ze, v4_6_1, fma(1.0 * oo2e, (v12_1_0 - rho_e * v12_1_1), acc[138]))));
+                acc[139] = fma(QCx, v12_8_0, fma(WQx, v12_8_1, fma(2.0 * oo2ze, v6_8_1, acc[139])));
+                acc[140] = fma(QCy, v12_7_0, fma(WQy, v12_7_1, fma(2.0 * oo2e, (v12_2_0 - rho_e * v12_2_1), acc[140])));
+                acc[141] = fma(QCy, v12_8_0, fma(WQy, v12_8_1, fma(1.0 * oo2e, (v12_3_0 - rho_e * v12_3_1), acc[141])));
+                acc[142] = fma(QCz, v12_8_0, fma(WQz, v12_8_1, fma(1.0 * oo2ze, v4_8_1, fma(1.0 * oo2e, (v12_2_0 - rho_e * v12_2_1), acc[142]))));
+                acc[143] = fma(QCz, v12_9_0, fma(WQz, v12_9_1, fma(1.0 * oo2ze, v4_9_1, fma(2.0 * oo2e, (v12_3_0 - rho_e * v12_3_1), acc[143]))));
+                acc[144] += (double)v13_4_0;
+                acc[145] += (double)v13_5_0;
+                acc[146] += (double)v13_6_0;
+                acc[147] += (double)v13_7_0;
+                acc[148] += (double)v13_8_0;
+                acc[149] += (double)v13_9_0;
+                acc[150] = fma(QCx, v13_4_0, fma(WQx, v13_4_1, fma(1.0 * oo2ze, v7_4_1, fma(2.0 * oo2e, (v13_1_0 - rho_e * v13_1_1), acc[150]))));
+                acc[151] = fma(QCx, v13_5_0, fma(WQx, v13_5_1, fma(1.0 * oo2ze, v7_5_1, fma(1.0 * oo2e, (v13_2_0 - rho_e * v13_2_1), acc[151]))));
+                acc[152] = fma(QCx, v13_6_0, fma(WQx, v13_6_1, fma(1.0 * oo2ze, v7_6_1, fma(1.0 * oo2e, (v13_3_0 - rho_e * v13_3_1), acc[152]))));
+                acc[153] = fma(QCy, v13_5_0, fma(WQy, v13_5_1, fma(2.0 * oo2ze, v5_5_1, fma(1.0 * oo2e, (v13_1_0 - rho_e * v13_1_1), acc[153]))));
+                acc[154] = fma(QCz, v13_6_0, fma(WQz, v13_6_1, fma(1.0 * oo2e, (v13_1_0 - rho_e * v13_1_1), acc[154])));
+                acc[155] = fma(QCx, v13_8_0, fma(WQx, v13_8_1, fma(1.0 * oo2ze, v7_8_1, acc[155])));
+                acc[156] = fma(QCy, v13_7_0, fma(WQy, v13_7_1, fma(2.0 * oo2ze, v5_7_1, fma(2.0 * oo2e, (v13_2_0 - rho_e * v13_2_1), acc[156]))));
+                acc[157] = fma(QCy, v13_8_0, fma(WQy, v13_8_1, fma(2.0 * oo2ze, v5_8_1, fma(1.0 * oo2e, (v13_3_0 - rho_e * v13_3_1), acc[157]))));
+                acc[158] = fma(QCz, v13_8_0, fma(WQz, v13_8_1, fma(1.0 * oo2e, (v13_2_0 - rho_e * v13_2_1), acc[158])));
+                acc[159] = fma(QCz, v13_9_0, fma(WQz, v13_9_1, fma(2.0 * oo2e, (v13_3_0 - rho_e * v13_3_1), acc[159])));
+                acc[160] += (double)v14_4_0;
+                acc[161] += (double)v14_5_0;
+                acc[162] += (double)v14_6_0;
+                acc[163] += (double)v14_7_0;
+                acc[164] += (double)v14_8_0;
+                acc[165] += (double)v14_9_0;
+                acc[166] = fma(QCx, v14_4_0, fma(WQx, v14_4_1, fma(1.0 * oo2ze, v9_4_1, fma(2.0 * oo2e, (v14_1_0 - rho_e * v14_1_1), acc[166]))));
+                acc[167] = fma(QCx, v14_5_0, fma(WQx, v14_5_1, fma(1.0 * oo2ze, v9_5_1, fma(1.0 * oo2e, (v14_2_0 - rho_e * v14_2_1), acc[167]))));
+                acc[168] = fma(QCx, v14_6_0, fma(WQx, v14_6_1, fma(1.0 * oo2ze, v9_6_1, fma(1.0 * oo2e, (v14_3_0 - rho_e * v14_3_1), acc[168]))));
+                acc[169] = fma(QCy, v14_5_0, fma(WQy, v14_5_1, fma(1.0 * oo2e, (v14_1_0 - rho_e * v14_1_1), acc[169])));
+                acc[170] = fma(QCz, v14_6_0, fma(WQz, v14_6_1, fma(2.0 * oo2ze, v6_6_1, fma(1.0 * oo2e, (v14_1_0 - rho_e * v14_1_1), acc[170]))));
+                acc[171] = fma(QCx, v14_8_0, fma(WQx, v14_8_1, fma(1.0 * oo2ze, v9_8_1, acc[171])));
+                acc[172] = fma(QCy, v14_7_0, fma(WQy, v14_7_1, fma(2.0 * oo2e, (v14_2_0 - rho_e * v14_2_1), acc[172])));
+                acc[173] = fma(QCy, v14_8_0, fma(WQy, v14_8_1, fma(1.0 * oo2e, (v14_3_0 - rho_e * v14_3_1), acc[173])));
+                acc[174] = fma(QCz, v14_8_0, fma(WQz, v14_8_1, fma(2.0 * oo2ze, v6_8_1, fma(1.0 * oo2e, (v14_2_0 - rho_e * v14_2_1), acc[174]))));
+                acc[175] = fma(QCz, v14_9_0, fma(WQz, v14_9_1, fma(2.0 * oo2ze, v6_9_1, fma(2.0 * oo2e, (v14_3_0 - rho_e * v14_3_1), acc[175]))));
+                acc[176] += (double)v15_4_0;
+                acc[177] += (double)v15_5_0;
+                acc[178] += (double)v15_6_0;
+                acc[179] += (double)v15_7_0;
+                acc[180] += (double)v15_8_0;
+                acc[181] += (double)v15_9_0;
+                acc[182] = fma(QCx, v15_4_0, fma(WQx, v15_4_1, fma(1.0 * oo2ze, v8_4_1, fma(2.0 * oo2e, (v15_1_0 - rho_e * v15_1_1), acc[182]))));
+                acc[183] = fma(QCx, v15_5_0, fma(WQx, v15_5_1, fma(1.0 * oo2ze, v8_5_1, fma(1.0 * oo2e, (v15_2_0 - rho_e * v15_2_1), acc[183]))));
+                acc[184] = fma(QCx, v15_6_0, fma(WQx, v15_6_1, fma(1.0 * oo2ze, v8_6_1, fma(1.0 * oo2e, (v15_3_0 - rho_e * v15_3_1), acc[184]))));
+                acc[185] = fma(QCy, v15_5_0, fma(WQy, v15_5_1, fma(1.0 * oo2ze, v6_5_1, fma(1.0 * oo2e, (v15_1_0 - rho_e * v15_1_1), acc[185]))));
+                acc[186] = fma(QCz, v15_6_0, fma(WQz, v15_6_1, fma(1.0 * oo2ze, v5_6_1, fma(1.0 * oo2e, (v15_1_0 - rho_e * v15_1_1), acc[186]))));
+                acc[187] = fma(QCx, v15_8_0, fma(WQx, v15_8_1, fma(1.0 * oo2ze, v8_8_1, acc[187])));
+                acc[188] = fma(QCy, v15_7_0, fma(WQy, v15_7_1, fma(1.0 * oo2ze, v6_7_1, fma(2.0 * oo2e, (v15_2_0 - rho_e * v15_2_1), acc[188]))));
+                acc[189] = fma(QCy, v15_8_0, fma(WQy, v15_8_1, fma(1.0 * oo2ze, v6_8_1, fma(1.0 * oo2e, (v15_3_0 - rho_e * v15_3_1), acc[189]))));
+                acc[190] = fma(QCz, v15_8_0, fma(WQz, v15_8_1, fma(1.0 * oo2ze, v5_8_1, fma(1.0 * oo2e, (v15_2_0 - rho_e * v15_2_1), acc[190]))));
+                acc[191] = fma(QCz, v15_9_0, fma(WQz, v15_9_1, fma(1.0 * oo2ze, v5_9_1, fma(2.0 * oo2e, (v15_3_0 - rho_e * v15_3_1), acc[191]))));
+                acc[192] += (double)v16_4_0;
+                acc[193] += (double)v16_5_0;
+                acc[194] += (double)v16_6_0;
+                acc[195] += (double)v16_7_0;
+                acc[196] += (double)v16_8_0;
+                acc[197] += (double)v16_9_0;
+                acc[198] = fma(QCx, v16_4_0, fma(WQx, v16_4_1, fma(2.0 * oo2e, (v16_1_0 - rho_e * v16_1_1), acc[198])));
+                acc[199] = fma(QCx, v16_5_0, fma(WQx, v16_5_1, fma(1.0 * oo2e, (v16_2_0 - rho_e * v16_2_1), acc[199])));
+                acc[200] = fma(QCx, v16_6_0, fma(WQx, v16_6_1, fma(1.0 * oo2e, (v16_3_0 - rho_e * v16_3_1), acc[200])));
+                acc[201] = fma(QCy, v16_5_0, fma(WQy, v16_5_1, fma(3.0 * oo2ze, v7_5_1, fma(1.0 * oo2e, (v16_1_0 - rho_e * v16_1_1), acc[201]))));
+                acc[202] = fma(QCz, v16_6_0, fma(WQz, v16_6_1, fma(1.0 * oo2e, (v16_1_0 - rho_e * v16_1_1), acc[202])));
+                acc[203] = fma(QCx, v16_8_0, fma(WQx, v16_8_1, acc[203]));
+                acc[204] = fma(QCy, v16_7_0, fma(WQy, v16_7_1, fma(3.0 * oo2ze, v7_7_1, fma(2.0 * oo2e, (v16_2_0 - rho_e * v16_2_1), acc[204]))));
+                acc[205] = fma(QCy, v16_8_0, fma(WQy, v16_8_1, fma(3.0 * oo2ze, v7_8_1, fma(1.0 * oo2e, (v16_3_0 - rho_e * v16_3_1), acc[205]))));
+                acc[206] = fma(QCz, v16_8_0, fma(WQz, v16_8_1, fma(1.0 * oo2e, (v16_2_0 - rho_e * v16_2_1), acc[206])));
+                acc[207] = fma(QCz, v16_9_0, fma(WQz, v16_9_1, fma(2.0 * oo2e, (v16_3_0 - rho_e * v16_3_1), acc[207])));
+                acc[208] += (double)v17_4_0;
+                acc[209] += (double)v17_5_0;
+                acc[210] += (double)v17_6_0;
+                acc[211] += (double)v17_7_0;
+                acc[212] += (double)v17_8_0;
+                acc[213] += (double)v17_9_0;
+                acc[214] = fma(QCx, v17_4_0, fma(WQx, v17_4_1, fma(2.0 * oo2e, (v17_1_0 - rho_e * v17_1_1), acc[214])));
+                acc[215] = fma(QCx, v17_5_0, fma(WQx, v17_5_1, fma(1.0 * oo2e, (v17_2_0 - rho_e * v17_2_1), acc[215])));
+                acc[216] = fma(QCx, v17_6_0, fma(WQx, v17_6_1, fma(1.0 * oo2e, (v17_3_0 - rho_e * v17_3_1), acc[216])));
+                acc[217] = fma(QCy, v17_5_0, fma(WQy, v17_5_1, fma(2.0 * oo2ze, v8_5_1, fma(1.0 * oo2e, (v17_1_0 - rho_e * v17_1_1), acc[217]))));
+                acc[218] = fma(QCz, v17_6_0, fma(WQz, v17_6_1, fma(1.0 * oo2ze, v7_6_1, fma(1.0 * oo2e, (v17_1_0 - rho_e * v17_1_1), acc[218]))));
+                acc[219] = fma(QCx, v17_8_0, fma(WQx, v17_8_1, acc[219]));
+                acc[220] = fma(QCy, v17_7_0, fma(WQy, v17_7_1, fma(2.0 * oo2ze, v8_7_1, fma(2.0 * oo2e, (v17_2_0 - rho_e * v17_2_1), acc[220]))));
+                acc[221] = fma(QCy, v17_8_0, fma(WQy, v17_8_1, fma(2.0 * oo2ze, v8_8_1, fma(1.0 * oo2e, (v17_3_0 - rho_e * v17_3_1), acc[221]))));
+                acc[222] = fma(QCz, v17_8_0, fma(WQz, v17_8_1, fma(1.0 * oo2ze, v7_8_1, fma(1.0 * oo2e, (v17_2_0 - rho_e * v17_2_1), acc[222]))));
+                acc[223] = fma(QCz, v17_9_0, fma(WQz, v17_9_1, fma(1.0 * oo2ze, v7_9_1, fma(2.0 * oo2e, (v17_3_0 - rho_e * v17_3_1), acc[223]))));
+                acc[224] += (double)v18_4_0;
+                acc[225] += (double)v18_5_0;
+                acc[226] += (double)v18_6_0;
+                acc[227] += (double)v18_7_0;
+                acc[228] += (double)v18_8_0;
+                acc[229] += (double)v18_9_0;
+                acc[230] = fma(QCx, v18_4_0, fma(WQx, v18_4_1, fma(2.0 * oo2e, (v18_1_0 - rho_e * v18_1_1), acc[230])));
+                acc[231] = fma(QCx, v18_5_0, fma(WQx, v18_5_1, fma(1.0 * oo2e, (v18_2_0 - rho_e * v18_2_1), acc[231])));
+                acc[232] = fma(QCx, v18_6_0, fma(WQx, v18_6_1, fma(1.0 * oo2e, (v18_3_0 - rho_e * v18_3_1), acc[232])));
+                acc[233] = fma(QCy, v18_5_0, fma(WQy, v18_5_1, fma(1.0 * oo2ze, v9_5_1, fma(1.0 * oo2e, (v18_1_0 - rho_e * v18_1_1), acc[233]))));
+                acc[234] = fma(QCz, v18_6_0, fma(WQz, v18_6_1, fma(2.0 * oo2ze, v8_6_1, fma(1.0 * oo2e, (v18_1_0 - rho_e * v18_1_1), acc[234]))));
+                acc[235] = fma(QCx, v18_8_0, fma(WQx, v18_8_1, acc[235]));
+                acc[236] = fma(QCy, v18_7_0, fma(WQy, v18_7_1, fma(1.0 * oo2ze, v9_7_1, fma(2.0 * oo2e, (v18_2_0 - rho_e * v18_2_1), acc[236]))));
+                acc[237] = fma(QCy, v18_8_0, fma(WQy, v18_8_1, fma(1.0 * oo2ze, v9_8_1, fma(1.0 * oo2e, (v18_3_0 - rho_e * v18_3_1), acc[237]))));
+                acc[238] = fma(QCz, v18_8_0, fma(WQz, v18_8_1, fma(2.0 * oo2ze, v8_8_1, fma(1.0 * oo2e, (v18_2_0 - rho_e * v18_2_1), acc[238]))));
+                acc[239] = fma(QCz, v18_9_0, fma(WQz, v18_9_1, fma(2.0 * oo2ze, v8_9_1, fma(2.0 * oo2e, (v18_3_0 - rho_e * v18_3_1), acc[239]))));
+                acc[240] += (double)v19_4_0;
+                acc[241] += (double)v19_5_0;
+                acc[242] += (double)v19_6_0;
+                acc[243] += (double)v19_7_0;
+                acc[244] += (double)v19_8_0;
+                acc[245] += (double)v19_9_0;
+                acc[246] = fma(QCx, v19_4_0, fma(WQx, v19_4_1, fma(2.0 * oo2e, (v19_1_0 - rho_e * v19_1_1), acc[246])));
+                acc[247] = fma(QCx, v19_5_0, fma(WQx, v19_5_1, fma(1.0 * oo2e, (v19_2_0 - rho_e * v19_2_1), acc[247])));
+                acc[248] = fma(QCx, v19_6_0, fma(WQx, v19_6_1, fma(1.0 * oo2e, (v19_3_0 - rho_e * v19_3_1), acc[248])));
+                acc[249] = fma(QCy, v19_5_0, fma(WQy, v19_5_1, fma(1.0 * oo2e, (v19_1_0 - rho_e * v19_1_1), acc[249])));
+                acc[250] = fma(QCz, v19_6_0, fma(WQz, v19_6_1, fma(3.0 * oo2ze, v9_6_1, fma(1.0 * oo2e, (v19_1_0 - rho_e * v19_1_1), acc[250]))));
+                acc[251] = fma(QCx, v19_8_0, fma(WQx, v19_8_1, acc[251]));
+                acc[252] = fma(QCy, v19_7_0, fma(WQy, v19_7_1, fma(2.0 * oo2e, (v19_2_0 - rho_e * v19_2_1), acc[252])));
+                acc[253] = fma(QCy, v19_8_0, fma(WQy, v19_8_1, fma(1.0 * oo2e, (v19_3_0 - rho_e * v19_3_1), acc[253])));
+                acc[254] = fma(QCz, v19_8_0, fma(WQz, v19_8_1, fma(3.0 * oo2ze, v9_8_1, fma(1.0 * oo2e, (v19_2_0 - rho_e * v19_2_1), acc[254]))));
+                acc[255] = fma(QCz, v19_9_0, fma(WQz, v19_9_1, fma(3.0 * oo2ze, v9_9_1, fma(2.0 * oo2e, (v19_3_0 - rho_e * v19_3_1), acc[255]))));
+                acc[256] += (double)v20_4_0;
+                acc[257] += (double)v20_5_0;
+                acc[258] += (double)v20_6_0;
+                acc[259] += (double)v20_7_0;
+                acc[260] += (double)v20_8_0;
+                acc[261] += (double)v20_9_0;
+                acc[262] = fma(QCx, v20_4_0, fma(WQx, v20_4_1, fma(4.0 * oo2ze, v10_4_1, fma(2.0 * oo2e, (v20_1_0 - rho_e * v20_1_1), acc[262]))));
+                acc[263] = fma(QCx, v20_5_0, fma(WQx, v20_5_1, fma(4.0 * oo2ze, v10_5_1, fma(1.0 * oo2e, (v20_2_0 - rho_e * v20_2_1), acc[263]))));
+                acc[264] = fma(QCx, v20_6_0, fma(WQx, v20_6_1, fma(4.0 * oo2ze, v10_6_1, fma(1.0 * oo2e, (v20_3_0 - rho_e * v20_3_1), acc[264]))));
+                acc[265] = fma(QCy, v20_5_0, fma(WQy, v20_5_1, fma(1.0 * oo2e, (v20_1_0 - rho_e * v20_1_1), acc[265])));
+                acc[266] = fma(QCz, v20_6_0, fma(WQz, v20_6_1, fma(1.0 * oo2e, (v20_1_0 - rho_e * v20_1_1), acc[266])));
+                acc[267] = fma(QCx, v20_8_0, fma(WQx, v20_8_1, fma(4.0 * oo2ze, v10_8_1, acc[267])));
+                acc[268] = fma(QCy, v20_7_0, fma(WQy, v20_7_1, fma(2.0 * oo2e, (v20_2_0 - rho_e * v20_2_1), acc[268])));
+                acc[269] = fma(QCy, v20_8_0, fma(WQy, v20_8_1, fma(1.0 * oo2e, (v20_3_0 - rho_e * v20_3_1), acc[269])));
+                acc[270] = fma(QCz, v20_8_0, fma(WQz, v20_8_1, fma(1.0 * oo2e, (v20_2_0 - rho_e * v20_2_1), acc[270])));
+                acc[271] = fma(QCz, v20_9_0, fma(WQz, v20_9_1, fma(2.0 * oo2e, (v20_3_0 - rho_e * v20_3_1), acc[271])));
+                acc[272] += (double)v21_4_0;
+                acc[273] += (double)v21_5_0;
+                acc[274] += (double)v21_6_0;
+                acc[275] += (double)v21_7_0;
+                acc[276] += (double)v21_8_0;
+                acc[277] += (double)v21_9_0;
+                acc[278] = fma(QCx, v21_4_0, fma(WQx, v21_4_1, fma(3.0 * oo2ze, v11_4_1, fma(2.0 * oo2e, (v21_1_0 - rho_e * v21_1_1), acc[278]))));
+                acc[279] = fma(QCx, v21_5_0, fma(WQx, v21_5_1, fma(3.0 * oo2ze, v11_5_1, fma(1.0 * oo2e, (v21_2_0 - rho_e * v21_2_1), acc[279]))));
+                acc[280] = fma(QCx, v21_6_0, fma(WQx, v21_6_1, fma(3.0 * oo2ze, v11_6_1, fma(1.0 * oo2e, (v21_3_0 - rho_e * v21_3_1), acc[280]))));
+                acc[281] = fma(QCy, v21_5_0, fma(WQy, v21_5_1, fma(1.0 * oo2ze, v10_5_1, fma(1.0 * oo2e, (v21_1_0 - rho_e * v21_1_1), acc[281]))));
+                acc[282] = fma(QCz, v21_6_0, fma(WQz, v21_6_1, fma(1.0 * oo2e, (v21_1_0 - rho_e * v21_1_1), acc[282])));
+                acc[283] = fma(QCx, v21_8_0, fma(WQx, v21_8_1, fma(3.0 * oo2ze, v11_8_1, acc[283])));
+                acc[284] = fma(QCy, v21_7_0, fma(WQy, v21_7_1, fma(1.0 * oo2ze, v10_7_1, fma(2.0 * oo2e, (v21_2_0 - rho_e * v21_2_1), acc[284]))));
+                acc[285] = fma(QCy, v21_8_0, fma(WQy, v21_8_1, fma(1.0 * oo2ze, v10_8_1, fma(1.0 * oo2e, (v21_3_0 - rho_e * v21_3_1), acc[285]))));
+                acc[286] = fma(QCz, v21_8_0, fma(WQz, v21_8_1, fma(1.0 * oo2e, (v21_2_0 - rho_e * v21_2_1), acc[286])));
+                acc[287] = fma(QCz, v21_9_0, fma(WQz, v21_9_1, fma(2.0 * oo2e, (v21_3_0 - rho_e * v21_3_1), acc[287])));
+                acc[288] += (double)v22_4_0;
+                acc[289] += (double)v22_5_0;
+                acc[290] += (double)v22_6_0;
+                acc[291] += (double)v22_7_0;
+                acc[292] += (double)v22_8_0;
+                acc[293] += (double)v22_9_0;
+                acc[294] = fma(QCx, v22_4_0, fma(WQx, v22_4_1, fma(3.0 * oo2ze, v12_4_1, fma(2.0 * oo2e, (v22_1_0 - rho_e * v22_1_1), acc[294]))));
+                acc[295] = fma(QCx, v22_5_0, fma(WQx, v22_5_1, fma(3.0 * oo2ze, v12_5_1, fma(1.0 * oo2e, (v22_2_0 - rho_e * v22_2_1), acc[295]))));
+                acc[296] = fma(QCx, v22_6_0, fma(WQx, v22_6_1, fma(3.0 * oo2ze, v12_6_1, fma(1.0 * oo2e, (v22_3_0 - rho_e * v22_3_1), acc[296]))));
+                acc[297] = fma(QCy, v22_5_0, fma(WQy, v22_5_1, fma(1.0 * oo2e, (v22_1_0 - rho_e * v22_1_1), acc[297])));
+                acc[298] = fma(QCz, v22_6_0, fma(WQz, v22_6_1, fma(1.0 * oo2ze, v10_6_1, fma(1.0 * oo2e, (v22_1_0 - rho_e * v22_1_1), acc[298]))));
+                acc[299] = fma(QCx, v22_8_0, fma(WQx, v22_8_1, fma(3.0 * oo2ze, v12_8_1, acc[299])));
+                acc[300] = fma(QCy, v22_7_0, fma(WQy, v22_7_1, fma(2.0 * oo2e, (v22_2_0 - rho_e * v22_2_1), acc[300])));
+                acc[301] = fma(QCy, v22_8_0, fma(WQy, v22_8_1, fma(1.0 * oo2e, (v22_3_0 - rho_e * v22_3_1), acc[301])));
+                acc[302] = fma(QCz, v22_8_0, fma(WQz, v22_8_1, fma(1.0 * oo2ze, v10_8_1, fma(1.0 * oo2e, (v22_2_0 - rho_e * v22_2_1), acc[302]))));
+                acc[303] = fma(QCz, v22_9_0, fma(WQz, v22_9_1, fma(1.0 * oo2ze, v10_9_1, fma(2.0 * oo2e, (v22_3_0 - rho_e * v22_3_1), acc[303]))));
+                acc[304] += (double)v23_4_0;
+                acc[305] += (double)v23_5_0;
+                acc[306] += (double)v23_6_0;
+                acc[307] += (double)v23_7_0;
+                acc[308] += (double)v23_8_0;
+                acc[309] += (double)v23_9_0;
+                acc[310] = fma(QCx, v23_4_0, fma(WQx, v23_4_1, fma(2.0 * oo2ze, v13_4_1, fma(2.0 * oo2e, (v23_1_0 - rho_e * v23_1_1), acc[310]))));
+                acc[311] = fma(QCx, v23_5_0, fma(WQx, v23_5_1, fma(2.0 * oo2ze, v13_5_1, fma(1.0 * oo2e, (v23_2_0 - rho_e * v23_2_1), acc[311]))));
+                acc[312] = fma(QCx, v23_6_0, fma(WQx, v23_6_1, fma(2.0 * oo2ze, v13_6_1, fma(1.0 * oo2e, (v23_3_0 - rho_e * v23_3_1), acc[312]))));
+                acc[313] = fma(QCy, v23_5_0, fma(WQy, v23_5_1, fma(2.0 * oo2ze, v11_5_1, fma(1.0 * oo2e, (v23_1_0 - rho_e * v23_1_1), acc[313]))));
+                acc[314] = fma(QCz, v23_6_0, fma(WQz, v23_6_1, fma(1.0 * oo2e, (v23_1_0 - rho_e * v23_1_1), acc[314])));
+                acc[315] = fma(QCx, v23_8_0, fma(WQx, v23_8_1, fma(2.0 * oo2ze, v13_8_1, acc[315])));
+                acc[316] = fma(QCy, v23_7_0, fma(WQy, v23_7_1, fma(2.0 * oo2ze, v11_7_1, fma(2.0 * oo2e, (v23_2_0 - rho_e * v23_2_1), acc[316]))));
+                acc[317] = fma(QCy, v23_8_0, fma(WQy, v23_8_1, fma(2.0 * oo2ze, v11_8_1, fma(1.0 * oo2e, (v23_3_0 - rho_e * v23_3_1), acc[317]))));
+                acc[318] = fma(QCz, v23_8_0, fma(WQz, v23_8_1, fma(1.0 * oo2e, (v23_2_0 - rho_e * v23_2_1), acc[318])));
+                acc[319] = fma(QCz, v23_9_0, fma(WQz, v23_9_1, fma(2.0 * oo2e, (v23_3_0 - rho_e * v23_3_1), acc[319])));
+                acc[320] += (double)v24_4_0;
+                acc[321] += (double)v24_5_0;
+                acc[322] += (double)v24_6_0;
+                acc[323] += (double)v24_7_0;
+                acc[324] += (double)v24_8_0;
+                acc[325] += (double)v24_9_0;
+                acc[326] = fma(QCx, v24_4_0, fma(WQx, v24_4_1, fma(2.0 * oo2ze, v15_4_1, fma(2.0 * oo2e, (v24_1_0 - rho_e * v24_1_1), acc[326]))));
+                acc[327] = fma(QCx, v24_5_0, fma(WQx, v24_5_1, fma(2.0 * oo2ze, v15_5_1, fma(1.0 * oo2e, (v24_2_0 - rho_e * v24_2_1), acc[327]))));
+                acc[328] = fma(QCx, v24_6_0, fma(WQx, v24_6_1, fma(2.0 * oo2ze, v15_6_1, fma(1.0 * oo2e, (v24_3_0 - rho_e * v24_3_1), acc[328]))));
+                acc[329] = fma(QCy, v24_5_0, fma(WQy, v24_5_1, fma(1.0 * oo2ze, v12_5_1, fma(1.0 * oo2e, (v24_1_0 - rho_e * v24_1_1), acc[329]))));
+                acc[330] = fma(QCz, v24_6_0, fma(WQz, v24_6_1, fma(1.0 * oo2ze, v11_6_1, fma(1.0 * oo2e, (v24_1_0 - rho_e * v24_1_1), acc[330]))));
+                acc[331] = fma(QCx, v24_8_0, fma(WQx, v24_8_1, fma(2.0 * oo2ze, v15_8_1, acc[331])));
+                acc[332] = fma(QCy, v24_7_0, fma(WQy, v24_7_1, fma(1.0 * oo2ze, v12_7_1, fma(2.0 * oo2e, (v24_2_0 - rho_e * v24_2_1), acc[332]))));
+                acc[333] = fma(QCy, v24_8_0, fma(WQy, v24_8_1, fma(1.0 * oo2ze, v12_8_1, fma(1.0 * oo2e, (v24_3_0 - rho_e * v24_3_1), acc[333]))));
+                acc[334] = fma(QCz, v24_8_0, fma(WQz, v24_8_1, fma(1.0 * oo2ze, v11_8_1, fma(1.0 * oo2e, (v24_2_0 - rho_e * v24_2_1), acc[334]))));
+                acc[335] = fma(QCz, v24_9_0, fma(WQz, v24_9_1, fma(1.0 * oo2ze, v11_9_1, fma(2.0 * oo2e, (v24_3_0 - rho_e * v24_3_1), acc[335]))));
+                acc[336] += (double)v25_4_0;
+                acc[337] += (double)v25_5_0;
+                acc[338] += (double)v25_6_0;
+                acc[339] += (double)v25_7_0;
+                acc[340] += (double)v25_8_0;
+                acc[341] += (double)v25_9_0;
+                acc[342] = fma(QCx, v25_4_0, fma(WQx, v25_4_1, fma(2.0 * oo2ze, v14_4_1, fma(2.0 * oo2e, (v25_1_0 - rho_e * v25_1_1), acc[342]))));
+                acc[343] = fma(QCx, v25_5_0, fma(WQx, v25_5_1, fma(2.0 * oo2ze, v14_5_1, fma(1.0 * oo2e, (v25_2_0 - rho_e * v25_2_1), acc[343]))));
+                acc[344] = fma(QCx, v25_6_0, fma(WQx, v25_6_1, fma(2.0 * oo2ze, v14_6_1, fma(1.0 * oo2e, (v25_3_0 - rho_e * v25_3_1), acc[344]))));
+                acc[345] = fma(QCy, v25_5_0, fma(WQy, v25_5_1, fma(1.0 * oo2e, (v25_1_0 - rho_e * v25_1_1), acc[345])));
+                acc[346] = fma(QCz, v25_6_0, fma(WQz, v25_6_1, fma(2.0 * oo2ze, v12_6_1, fma(1.0 * oo2e, (v25_1_0 - rho_e * v25_1_1), acc[346]))));
+                acc[347] = fma(QCx, v25_8_0, fma(WQx, v25_8_1, fma(2.0 * oo2ze, v14_8_1, acc[347])));
+                acc[348] = fma(QCy, v25_7_0, fma(WQy, v25_7_1, fma(2.0 * oo2e, (v25_2_0 - rho_e * v25_2_1), acc[348])));
+                acc[349] = fma(QCy, v25_8_0, fma(WQy, v25_8_1, fma(1.0 * oo2e, (v25_3_0 - rho_e * v25_3_1), acc[349])));
+                acc[350] = fma(QCz, v25_8_0, fma(WQz, v25_8_1, fma(2.0 * oo2ze, v12_8_1, fma(1.0 * oo2e, (v25_2_0 - rho_e * v25_2_1), acc[350]))));
+                acc[351] = fma(QCz, v25_9_0, fma(WQz, v25_9_1, fma(2.0 * oo2ze, v12_9_1, fma(2.0 * oo2e, (v25_3_0 - rho_e * v25_3_1), acc[351]))));
+                acc[352] += (double)v26_4_0;
+                acc[353] += (double)v26_5_0;
+                acc[354] += (double)v26_6_0;
+                acc[355] += (double)v26_7_0;
+                acc[356] += (double)v26_8_0;
+                acc[357] += (double)v26_9_0;
+                acc[358] = fma(QCx, v26_4_0, fma(WQx, v26_4_1, fma(1.0 * oo2ze, v16_4_1, fma(2.0 * oo2e, (v26_1_0 - rho_e * v26_1_1), acc[358]))));
+                acc[359] = fma(QCx, v26_5_0, fma(WQx, v26_5_1, fma(1.0 * oo2ze, v16_5_1, fma(1.0 * oo2e, (v26_2_0 - rho_e * v26_2_1), acc[359]))));
+                acc[360] = fma(QCx, v26_6_0, fma(WQx, v26_6_1, fma(1.0 * oo2ze, v16_6_1, fma(1.0 * oo2e, (v26_3_0 - rho_e * v26_3_1), acc[360]))));
+                acc[361] = fma(QCy, v26_5_0, fma(WQy, v26_5_1, fma(3.0 * oo2ze, v13_5_1, fma(1.0 * oo2e, (v26_1_0 - rho_e * v26_1_1), acc[361]))));
+                acc[362] = fma(QCz, v26_6_0, fma(WQz, v26_6_1, fma(1.0 * oo2e, (v26_1_0 - rho_e * v26_1_1), acc[362])));
+                acc[363] = fma(QCx, v26_8_0, fma(WQx, v26_8_1, fma(1.0 * oo2ze, v16_8_1, acc[363])));
+                acc[364] = fma(QCy, v26_7_0, fma(WQy, v26_7_1, fma(3.0 * oo2ze, v13_7_1, fma(2.0 * oo2e, (v26_2_0 - rho_e * v26_2_1), acc[364]))));
+                acc[365] = fma(QCy, v26_8_0, fma(WQy, v26_8_1, fma(3.0 * oo2ze, v13_8_1, fma(1.0 * oo2e, (v26_3_0 - rho_e * v26_3_1), acc[365]))));
+                acc[366] = fma(QCz, v26_8_0, fma(WQz, v26_8_1, fma(1.0 * oo2e, (v26_2_0 - rho_e * v26_2_1), acc[366])));
+                acc[367] = fma(QCz, v26_9_0, fma(WQz, v26_9_1, fma(2.0 * oo2e, (v26_3_0 - rho_e * v26_3_1), acc[367])));
+                acc[368] += (double)v27_4_0;
+                acc[369] += (double)v27_5_0;
+                acc[370] += (double)v27_6_0;
+                acc[371] += (double)v27_7_0;
+                acc[372] += (double)v27_8_0;
+                acc[373] += (double)v27_9_0;
+                acc[374] = fma(QCx, v27_4_0, fma(WQx, v27_4_1, fma(1.0 * oo2ze, v17_4_1, fma(2.0 * oo2e, (v27_1_0 - rho_e * v27_1_1), acc[374]))));
+                acc[375] = fma(QCx, v27_5_0, fma(WQx, v27_5_1, fma(1.0 * oo2ze, v17_5_1, fma(1.0 * oo2e, (v27_2_0 - rho_e * v27_2_1), acc[375]))));
+                acc[376] = fma(QCx, v27_6_0, fma(WQx, v27_6_1, fma(1.0 * oo2ze, v17_6_1, fma(1.0 * oo2e, (v27_3_0 - rho_e * v27_3_1), acc[376]))));
+                acc[377] = fma(QCy, v27_5_0, fma(WQy, v27_5_1, fma(2.0 * oo2ze, v15_5_1, fma(1.0 * oo2e, (v27_1_0 - rho_e * v27_1_1), acc[377]))));
+                acc[378] = fma(QCz, v27_6_0, fma(WQz, v27_6_1, fma(1.0 * oo2ze, v13_6_1, fma(1.0 * oo2e, (v27_1_0 - rho_e * v27_1_1), acc[378]))));
+                acc[379] = fma(QCx, v27_8_0, fma(WQx, v27_8_1, fma(1.0 * oo2ze, v17_8_1, acc[379])));
+                acc[380] = fma(QCy, v27_7_0, fma(WQy, v27_7_1, fma(2.0 * oo2ze, v15_7_1, fma(2.0 * oo2e, (v27_2_0 - rho_e * v27_2_1), acc[380]))));
+                acc[381] = fma(QCy, v27_8_0, fma(WQy, v27_8_1, fma(2.0 * oo2ze, v15_8_1, fma(1.0 * oo2e, (v27_3_0 - rho_e * v27_3_1), acc[381]))));
+                acc[382] = fma(QCz, v27_8_0, fma(WQz, v27_8_1, fma(1.0 * oo2ze, v13_8_1, fma(1.0 * oo2e, (v27_2_0 - rho_e * v27_2_1), acc[382]))));
+                acc[383] = fma(QCz, v27_9_0, fma(WQz, v27_9_1, fma(1.0 * oo2ze, v13_9_1, fma(2.0 * oo2e, (v27_3_0 - rho_e * v27_3_1), acc[383]))));
+                acc[384] += (double)v28_4_0;
+                acc[385] += (double)v28_5_0;
+                acc[386] += (double)v28_6_0;
+                acc[387] += (double)v28_7_0;
+                acc[388] += (double)v28_8_0;
+                acc[389] += (double)v28_9_0;
+                acc[390] = fma(QCx, v28_4_0, fma(WQx, v28_4_1, fma(1.0 * oo2ze, v18_4_1, fma(2.0 * oo2e, (v28_1_0 - rho_e * v28_1_1), acc[390]))));
+                acc[391] = fma(QCx, v28_5_0, fma(WQx, v28_5_1, fma(1.0 * oo2ze, v18_5_1, fma(1.0 * oo2e, (v28_2_0 - rho_e * v28_2_1), acc[391]))));
+                acc[392] = fma(QCx, v28_6_0, fma(WQx, v28_6_1, fma(1.0 * oo2ze, v18_6_1, fma(1.0 * oo2e, (v28_3_0 - rho_e * v28_3_1), acc[392]))));
+                acc[393] = fma(QCy, v28_5_0, fma(WQy, v28_5_1, fma(1.0 * oo2ze, v14_5_1, fma(1.0 * oo2e, (v28_1_0 - rho_e * v28_1_1), acc[393]))));
+                acc[394] = fma(QCz, v28_6_0, fma(WQz, v28_6_1, fma(2.0 * oo2ze, v15_6_1, fma(1.0 * oo2e, (v28_1_0 - rho_e * v28_1_1), acc[394]))));
+                acc[395] = fma(QCx, v28_8_0, fma(WQx, v28_8_1, fma(1.0 * oo2ze, v18_8_1, acc[395])));
+                acc[396] = fma(QCy, v28_7_0, fma(WQy, v28_7_1, fma(1.0 * oo2ze, v14_7_1, fma(2.0 * oo2e, (v28_2_0 - rho_e * v28_2_1), acc[396]))));
+                acc[397] = fma(QCy, v28_8_0, fma(WQy, v28_8_1, fma(1.0 * oo2ze, v14_8_1, fma(1.0 * oo2e, (v28_3_0 - rho_e * v28_3_1), acc[397]))));
+                acc[398] = fma(QCz, v28_8_0, fma(WQz, v28_8_1, fma(2.0 * oo2ze, v15_8_1, fma(1.0 * oo2e, (v28_2_0 - rho_e * v28_2_1), acc[398]))));
+                acc[399] = fma(QCz, v28_9_0, fma(WQz, v28_9_1, fma(2.0 * oo2ze, v15_9_1, fma(2.0 * oo2e, (v28_3_0 - rho_e * v28_3_1), acc[399]))));
+                acc[400] += (double)v29_4_0;
+                acc[401] += (double)v29_5_0;
+                acc[402] += (double)v29_6_0;
+                acc[403] += (double)v29_7_0;
+                acc[404] += (double)v29_8_0;
+                acc[405] += (double)v29_9_0;
+                acc[406] = fma(QCx, v29_4_0, fma(WQx, v29_4_1, fma(1.0 * oo2ze, v19_4_1, fma(2.0 * oo2e, (v29_1_0 - rho_e * v29_1_1), acc[406]))));
+                acc[407] = fma(QCx, v29_5_0, fma(WQx, v29_5_1, fma(1.0 * oo2ze, v19_5_1, fma(1.0 * oo2e, (v29_2_0 - rho_e * v29_2_1), acc[407]))));
+                acc[408] = fma(QCx, v29_6_0, fma(WQx, v29_6_1, fma(1.0 * oo2ze, v19_6_1, fma(1.0 * oo2e, (v29_3_0 - rho_e * v29_3_1), acc[408]))));
+                acc[409] = fma(QCy, v29_5_0, fma(WQy, v29_5_1, fma(1.0 * oo2e, (v29_1_0 - rho_e * v29_1_1), acc[409])));
+                acc[410] = fma(QCz, v29_6_0, fma(WQz, v29_6_1, fma(3.0 * oo2ze, v14_6_1, fma(1.0 * oo2e, (v29_1_0 - rho_e * v29_1_1), acc[410]))));
+                acc[411] = fma(QCx, v29_8_0, fma(WQx, v29_8_1, fma(1.0 * oo2ze, v19_8_1, acc[411])));
+                acc[412] = fma(QCy, v29_7_0, fma(WQy, v29_7_1, fma(2.0 * oo2e, (v29_2_0 - rho_e * v29_2_1), acc[412])));
+                acc[413] = fma(QCy, v29_8_0, fma(WQy, v29_8_1, fma(1.0 * oo2e, (v29_3_0 - rho_e * v29_3_1), acc[413])));
+                acc[414] = fma(QCz, v29_8_0, fma(WQz, v29_8_1, fma(3.0 * oo2ze, v14_8_1, fma(1.0 * oo2e, (v29_2_0 - rho_e * v29_2_1), acc[414]))));
+                acc[415] = fma(QCz, v29_9_0, fma(WQz, v29_9_1, fma(3.0 * oo2ze, v14_9_1, fma(2.0 * oo2e, (v29_3_0 - rho_e * v29_3_1), acc[415]))));
+                acc[416] += (double)v30_4_0;
+                acc[417] += (double)v30_5_0;
+                acc[418] += (double)v30_6_0;
+                acc[419] += (double)v30_7_0;
+                acc[420] += (double)v30_8_0;
+                acc[421] += (double)v30_9_0;
+                acc[422] = fma(QCx, v30_4_0, fma(WQx, v30_4_1, fma(2.0 * oo2e, (v30_1_0 - rho_e * v30_1_1), acc[422])));
+                acc[423] = fma(QCx, v30_5_0, fma(WQx, v30_5_1, fma(1.0 * oo2e, (v30_2_0 - rho_e * v30_2_1), acc[423])));
+                acc[424] = fma(QCx, v30_6_0, fma(WQx, v30_6_1, fma(1.0 * oo2e, (v30_3_0 - rho_e * v30_3_1), acc[424])));
+                acc[425] = fma(QCy, v30_5_0, fma(WQy, v30_5_1, fma(4.0 * oo2ze, v16_5_1, fma(1.0 * oo2e, (v30_1_0 - rho_e * v30_1_1), acc[425]))));
+                acc[426] = fma(QCz, v30_6_0, fma(WQz, v30_6_1, fma(1.0 * oo2e, (v30_1_0 - rho_e * v30_1_1), acc[426])));
+                acc[427] = fma(QCx, v30_8_0, fma(WQx, v30_8_1, acc[427]));
+                acc[428] = fma(QCy, v30_7_0, fma(WQy, v30_7_1, fma(4.0 * oo2ze, v16_7_1, fma(2.0 * oo2e, (v30_2_0 - rho_e * v30_2_1), acc[428]))));
+                acc[429] = fma(QCy, v30_8_0, fma(WQy, v30_8_1, fma(4.0 * oo2ze, v16_8_1, fma(1.0 * oo2e, (v30_3_0 - rho_e * v30_3_1), acc[429]))));
+                acc[430] = fma(QCz, v30_8_0, fma(WQz, v30_8_1, fma(1.0 * oo2e, (v30_2_0 - rho_e * v30_2_1), acc[430])));
+                acc[431] = fma(QCz, v30_9_0, fma(WQz, v30_9_1, fma(2.0 * oo2e, (v30_3_0 - rho_e * v30_3_1), acc[431])));
+                acc[432] += (double)v31_4_0;
+                acc[433] += (double)v31_5_0;
+                acc[434] += (double)v31_6_0;
+                acc[435] += (double)v31_7_0;
+                acc[436] += (double)v31_8_0;
+                acc[437] += (double)v31_9_0;
+                acc[438] = fma(QCx, v31_4_0, fma(WQx, v31_4_1, fma(2.0 * oo2e, (v31_1_0 - rho_e * v31_1_1), acc[438])));
+                acc[439] = fma(QCx, v31_5_0, fma(WQx, v31_5_1, fma(1.0 * oo2e, (v31_2_0 - rho_e * v31_2_1), acc[439])));
+                acc[440] = fma(QCx, v31_6_0, fma(WQx, v31_6_1, fma(1.0 * oo2e, (v31_3_0 - rho_e * v31_3_1), acc[440])));
+                acc[441] = fma(QCy, v31_5_0, fma(WQy, v31_5_1, fma(3.0 * oo2ze, v17_5_1, fma(1.0 * oo2e, (v31_1_0 - rho_e * v31_1_1), acc[441]))));
+                acc[442] = fma(QCz, v31_6_0, fma(WQz, v31_6_1, fma(1.0 * oo2ze, v16_6_1, fma(1.0 * oo2e, (v31_1_0 - rho_e * v31_1_1), acc[442]))));
+                acc[443] = fma(QCx, v31_8_0, fma(WQx, v31_8_1, acc[443]));
+                acc[444] = fma(QCy, v31_7_0, fma(WQy, v31_7_1, fma(3.0 * oo2ze, v17_7_1, fma(2.0 * oo2e, (v31_2_0 - rho_e * v31_2_1), acc[444]))));
+                acc[445] = fma(QCy, v31_8_0, fma(WQy, v31_8_1, fma(3.0 * oo2ze, v17_8_1, fma(1.0 * oo2e, (v31_3_0 - rho_e * v31_3_1), acc[445]))));
+                acc[446] = fma(QCz, v31_8_0, fma(WQz, v31_8_1, fma(1.0 * oo2ze, v16_8_1, fma(1.0 * oo2e, (v31_2_0 - rho_e * v31_2_1), acc[446]))));
+                acc[447] = fma(QCz, v31_9_0, fma(WQz, v31_9_1, fma(1.0 * oo2ze, v16_9_1, fma(2.0 * oo2e, (v31_3_0 - rho_e * v31_3_1), acc[447]))));
+                acc[448] += (double)v32_4_0;
+                acc[449] += (double)v32_5_0;
+                acc[450] += (double)v32_6_0;
+                acc[451] += (double)v32_7_0;
+                acc[452] += (double)v32_8_0;
+                acc[453] += (double)v32_9_0;
+                acc[454] = fma(QCx, v32_4_0, fma(WQx, v32_4_1, fma(2.0 * oo2e, (v32_1_0 - rho_e * v32_1_1), acc[454])));
+                acc[455] = fma(QCx, v32_5_0, fma(WQx, v32_5_1, fma(1.0 * oo2e, (v32_2_0 - rho_e * v32_2_1), acc[455])));
+                acc[456] = fma(QCx, v32_6_0, fma(WQx, v32_6_1, fma(1.0 * oo2e, (v32_3_0 - rho_e * v32_3_1), acc[456])));
+                acc[457] = fma(QCy, v32_5_0, fma(WQy, v32_5_1, fma(2.0 * oo2ze, v18_5_1, fma(1.0 * oo2e, (v32_1_0 - rho_e * v32_1_1), acc[457]))));
+                acc[458] = fma(QCz, v32_6_0, fma(WQz, v32_6_1, fma(2.0 * oo2ze, v17_6_1, fma(1.0 * oo2e, (v32_1_0 - rho_e * v32_1_1), acc[458]))));
+                acc[459] = fma(QCx, v32_8_0, fma(WQx, v32_8_1, acc[459]));
+                acc[460] = fma(QCy, v32_7_0, fma(WQy, v32_7_1, fma(2.0 * oo2ze, v18_7_1, fma(2.0 * oo2e, (v32_2_0 - rho_e * v32_2_1), acc[460]))));
+                acc[461] = fma(QCy, v32_8_0, fma(WQy, v32_8_1, fma(2.0 * oo2ze, v18_8_1, fma(1.0 * oo2e, (v32_3_0 - rho_e * v32_3_1), acc[461]))));
+                acc[462] = fma(QCz, v32_8_0, fma(WQz, v32_8_1, fma(2.0 * oo2ze, v17_8_1, fma(1.0 * oo2e, (v32_2_0 - rho_e * v32_2_1), acc[462]))));
+                acc[463] = fma(QCz, v32_9_0, fma(WQz, v32_9_1, fma(2.0 * oo2ze, v17_9_1, fma(2.0 * oo2e, (v32_3_0 - rho_e * v32_3_1), acc[463]))));
+                acc[464] += (double)v33_4_0;
+                acc[465] += (double)v33_5_0;
+                acc[466] += (double)v33_6_0;
+                acc[467] += (double)v33_7_0;
+                acc[468] += (double)v33_8_0;
+                acc[469] += (double)v33_9_0;
+                acc[470] = fma(QCx, v33_4_0, fma(WQx, v33_4_1, fma(2.0 * oo2e, (v33_1_0 - rho_e * v33_1_1), acc[470])));
+                acc[471] = fma(QCx, v33_5_0, fma(WQx, v33_5_1, fma(1.0 * oo2e, (v33_2_0 - rho_e * v33_2_1), acc[471])));
+                acc[472] = fma(QCx, v33_6_0, fma(WQx, v33_6_1, fma(1.0 * oo2e, (v33_3_0 - rho_e * v33_3_1), acc[472])));
+                acc[473] = fma(QCy, v33_5_0, fma(WQy, v33_5_1, fma(1.0 * oo2ze, v19_5_1, fma(1.0 * oo2e, (v33_1_0 - rho_e * v33_1_1), acc[473]))));
+                acc[474] = fma(QCz, v33_6_0, fma(WQz, v33_6_1, fma(3.0 * oo2ze, v18_6_1, fma(1.0 * oo2e, (v33_1_0 - rho_e * v33_1_1), acc[474]))));
+                acc[475] = fma(QCx, v33_8_0, fma(WQx, v33_8_1, acc[475]));
+                acc[476] = fma(QCy, v33_7_0, fma(WQy, v33_7_1, fma(1.0 * oo2ze, v19_7_1, fma(2.0 * oo2e, (v33_2_0 - rho_e * v33_2_1), acc[476]))));
+                acc[477] = fma(QCy, v33_8_0, fma(WQy, v33_8_1, fma(1.0 * oo2ze, v19_8_1, fma(1.0 * oo2e, (v33_3_0 - rho_e * v33_3_1), acc[477]))));
+                acc[478] = fma(QCz, v33_8_0, fma(WQz, v33_8_1, fma(3.0 * oo2ze, v18_8_1, fma(1.0 * oo2e, (v33_2_0 - rho_e * v33_2_1), acc[478]))));
+                acc[479] = fma(QCz, v33_9_0, fma(WQz, v33_9_1, fma(3.0 * oo2ze, v18_9_1, fma(2.0 * oo2e, (v33_3_0 - rho_e * v33_3_1), acc[479]))));
+                acc[480] += (double)v34_4_0;
+                acc[481] += (double)v34_5_0;
+                acc[482] += (double)v34_6_0;
+                acc[483] += (double)v34_7_0;
+                acc[484] += (double)v34_8_0;
+                acc[485] += (double)v34_9_0;
+                acc[486] = fma(QCx, v34_4_0, fma(WQx, v34_4_1, fma(2.0 * oo2e, (v34_1_0 - rho_e * v34_1_1), acc[486])));
+                acc[487] = fma(QCx, v34_5_0, fma(WQx, v34_5_1, fma(1.0 * oo2e, (v34_2_0 - rho_e * v34_2_1), acc[487])));
+                acc[488] = fma(QCx, v34_6_0, fma(WQx, v34_6_1, fma(1.0 * oo2e, (v34_3_0 - rho_e * v34_3_1), acc[488])));
+                acc[489] = fma(QCy, v34_5_0, fma(WQy, v34_5_1, fma(1.0 * oo2e, (v34_1_0 - rho_e * v34_1_1), acc[489])));
+                acc[490] = fma(QCz, v34_6_0, fma(WQz, v34_6_1, fma(4.0 * oo2ze, v19_6_1, fma(1.0 * oo2e, (v34_1_0 - rho_e * v34_1_1), acc[490]))));
+                acc[491] = fma(QCx, v34_8_0, fma(WQx, v34_8_1, acc[491]));
+                acc[492] = fma(QCy, v34_7_0, fma(WQy, v34_7_1, fma(2.0 * oo2e, (v34_2_0 - rho_e * v34_2_1), acc[492])));
+                acc[493] = fma(QCy, v34_8_0, fma(WQy, v34_8_1, fma(1.0 * oo2e, (v34_3_0 - rho_e * v34_3_1), acc[493])));
+                acc[494] = fma(QCz, v34_8_0, fma(WQz, v34_8_1, fma(4.0 * oo2ze, v19_8_1, fma(1.0 * oo2e, (v34_2_0 - rho_e * v34_2_1), acc[494]))));
+                acc[495] = fma(QCz, v34_9_0, fma(WQz, v34_9_1, fma(4.0 * oo2ze, v19_9_1, fma(2.0 * oo2e, (v34_3_0 - rho_e * v34_3_1), acc[495]))));
+            } else {
+                acc[0] += (double)v4_4_0;
+                acc[1] += (double)v4_5_0;
+                acc[2] += (double)v4_6_0;
+                acc[3] += (double)v4_7_0;
+                acc[4] += (double)v4_8_0;
+                acc[5] += (double)v4_9_0;
+                const VT v4_10_0 = QCx * v4_4_0 + WQx * v4_4_1 + (VT)2.0 * oo2ze * v1_4_1 + (VT)2.0 * oo2e * (v4_1_0 - rho_e * v4_1_1);
+                acc[6] += (double)v4_10_0;
+                const VT v4_11_0 = QCx * v4_5_0 + WQx * v4_5_1 + (VT)2.0 * oo2ze * v1_5_1 + (VT)1.0 * oo2e * (v4_2_0 - rho_e * v4_2_1);
+                acc[7] += (double)v4_11_0;
+                const VT v4_12_0 = QCx * v4_6_0 + WQx * v4_6_1 + (VT)2.0 * oo2ze * v1_6_1 + (VT)1.0 * oo2e * (v4_3_0 - rho_e * v4_3_1);
+                acc[8] += (double)v4_12_0;
+                const VT v4_13_0 = QCy * v4_5_0 + WQy * v4_5_1 + (VT)1.0 * oo2e * (v4_1_0 - rho_e * v4_1_1);
+                acc[9] += (double)v4_13_0;
+                const VT v4_14_0 = QCz * v4_6_0 + WQz * v4_6_1 + (VT)1.0 * oo2e * (v4_1_0 - rho_e * v4_1_1);
+                acc[10] += (double)v4_14_0;
+                const VT v4_15_0 = QCx * v4_8_0 + WQx * v4_8_1 + (VT)2.0 * oo2ze * v1_8_1;
+                acc[11] += (double)v4_15_0;
+                const VT v4_16_0 = QCy * v4_7_0 + WQy * v4_7_1 + (VT)2.0 * oo2e * (v4_2_0 - rho_e * v4_2_1);
+                acc[12] += (double)v4_16_0;
+                const VT v4_17_0 = QCy * v4_8_0 + WQy * v4_8_1 + (VT)1.0 * oo2e * (v4_3_0 - rho_e * v4_3_1);
+                acc[13] += (double)v4_17_0;
+                const VT v4_18_0 = QCz * v4_8_0 + WQz * v4_8_1 + (VT)1.0 * oo2e * (v4_2_0 - rho_e * v4_2_1);
+                acc[14] += (double)v4_18_0;
+                const VT v4_19_0 = QCz * v4_9_0 + WQz * v4_9_1 + (VT)2.0 * oo2e * (v4_3_0 - rho_e * v4_3_1);
+                acc[15] += (double)v4_19_0;
+                acc[16] += (double)v5_4_0;
+                acc[17] += (double)v5_5_0;
+                acc[18] += (double)v5_6_0;
+                acc[19] += (double)v5_7_0;
+                acc[20] += (double)v5_8_0;
+                acc[21] += (double)v5_9_0;
+                const VT v5_10_0 = QCx * v5_4_0 + WQx * v5_4_1 + (VT)1.0 * oo2ze * v2_4_1 + (VT)2.0 * oo2e * (v5_1_0 - rho_e * v5_1_1);
+                acc[22] += (double)v5_10_0;
+                const VT v5_11_0 = QCx * v5_5_0 + WQx * v5_5_1 + (VT)1.0 * oo2ze * v2_5_1 + (VT)1.0 * oo2e * (v5_2_0 - rho_e * v5_2_1);
+                acc[23] += (double)v5_11_0;
+                const VT v5_12_0 = QCx * v5_6_0 + WQx * v5_6_1 + (VT)1.0 * oo2ze * v2_6_1 + (VT)1.0 * oo2e * (v5_3_0 - rho_e * v5_3_1);
+                acc[24] += (double)v5_12_0;
+                const VT v5_13_0 = QCy * v5_5_0 + WQy * v5_5_1 + (VT)1.0 * oo2ze * v1_5_1 + (VT)1.0 * oo2e * (v5_1_0 - rho_e * v5_1_1);
+                acc[25] += (double)v5_13_0;
+                const VT v5_14_0 = QCz * v5_6_0 + WQz * v5_6_1 + (VT)1.0 * oo2e * (v5_1_0 - rho_e * v5_1_1);
+                acc[26] += (double)v5_14_0;
+                const VT v5_15_0 = QCx * v5_8_0 + WQx * v5_8_1 + (VT)1.0 * oo2ze * v2_8_1;
+                acc[27] += (double)v5_15_0;
+                const VT v5_16_0 = QCy * v5_7_0 + WQy * v5_7_1 + (VT)1.0 * oo2ze * v1_7_1 + (VT)2.0 * oo2e * (v5_2_0 - rho_e * v5_2_1);
+                acc[28] += (double)v5_16_0;
+                const VT v5_17_0 = QCy * v5_8_0 + WQy * v5_8_1 + (VT)1.0 * oo2ze * v1_8_1 + (VT)1.0 * oo2e * (v5_3_0 - rho_e * v5_3_1);
+                acc[29] += (double)v5_17_0;
+                const VT v5_18_0 = QCz * v5_8_0 + WQz * v5_8_1 + (VT)1.0 * oo2e * (v5_2_0 - rho_e * v5_2_1);
+                acc[30] += (double)v5_18_0;
+                const VT v5_19_0 = QCz * v5_9_0 + WQz * v5_9_1 + (VT)2.0 * oo2e * (v5_3_0 - rho_e * v5_3_1);
+                acc[31] += (double)v5_19_0;
+                acc[32] += (double)v6_4_0;
+                acc[33] += (double)v6_5_0;
+                acc[34] += (double)v6_6_0;
+                acc[35] += (double)v6_7_0;
+                acc[36] += (double)v6_8_0;
+                acc[37] += (double)v6_9_0;
+                const VT v6_10_0 = QCx * v6_4_0 + WQx * v6_4_1 + (VT)1.0 * oo2ze * v3_4_1 + (VT)2.0 * oo2e * (v6_1_0 - rho_e * v6_1_1);
+                acc[38] += (double)v6_10_0;
+                const VT v6_11_0 = QCx * v6_5_0 + WQx * v6_5_1 + (VT)1.0 * oo2ze * v3_5_1 + (VT)1.0 * oo2e * (v6_2_0 - rho_e * v6_2_1);
+                acc[39] += (double)v6_11_0;
+                const VT v6_12_0 = QCx * v6_6_0 + WQx * v6_6_1 + (VT)1.0 * oo2ze * v3_6_1 + (VT)1.0 * oo2e * (v6_3_0 - rho_e * v6_3_1);
+                acc[40] += (double)v6_12_0;
+                const VT v6_13_0 = QCy * v6_5_0 + WQy * v6_5_1 + (VT)1.0 * oo2e * (v6_1_0 - rho_e * v6_1_1);
+                acc[41] += (double)v6_13_0;
+                const VT v6_14_0 = QCz * v6_6_0 + WQz * v6_6_1 + (VT)1.0 * oo2ze * v1_6_1 + (VT)1.0 * oo2e * (v6_1_0 - rho_e * v6_1_1);
+                acc[42] += (double)v6_14_0;
+                const VT v6_15_0 = QCx * v6_8_0 + WQx * v6_8_1 + (VT)1.0 * oo2ze * v3_8_1;
+                acc[43] += (double)v6_15_0;
+                const VT v6_16_0 = QCy * v6_7_0 + WQy * v6_7_1 + (VT)2.0 * oo2e * (v6_2_0 - rho_e * v6_2_1);
+                acc[44] += (double)v6_16_0;
+                const VT v6_17_0 = QCy * v6_8_0 + WQy * v6_8_1 + (VT)1.0 * oo2e * (v6_3_0 - rho_e * v6_3_1);
+                acc[45] += (double)v6_17_0;
+                const VT v6_18_0 = QCz * v6_8_0 + WQz * v6_8_1 + (VT)1.0 * oo2ze * v1_8_1 + (VT)1.0 * oo2e * (v6_2_0 - rho_e * v6_2_1);
+                acc[46] += (double)v6_18_0;
+                const VT v6_19_0 = QCz * v6_9_0 + WQz * v6_9_1 + (VT)1.0 * oo2ze * v1_9_1 + (VT)2.0 * oo2e * (v6_3_0 - rho_e * v6_3_1);
+                acc[47] += (double)v6_19_0;
+                acc[48] += (double)v7_4_0;
+                acc[49] += (double)v7_5_0;
+                acc[50] += (double)v7_6_0;
+                acc[51] += (double)v7_7_0;
+                acc[52] += (double)v7_8_0;
+                acc[53] += (double)v7_9_0;
+                const VT v7_10_0 = QCx * v7_4_0 + WQx * v7_4_1 + (VT)2.0 * oo2e * (v7_1_0 - rho_e * v7_1_1);
+                acc[54] += (double)v7_10_0;
+                const VT v7_11_0 = QCx * v7_5_0 + WQx * v7_5_1 + (VT)1.0 * oo2e * (v7_2_0 - rho_e * v7_2_1);
+                acc[55] += (double)v7_11_0;
+                const VT v7_12_0 = QCx * v7_6_0 + WQx * v7_6_1 + (VT)1.0 * oo2e * (v7_3_0 - rho_e * v7_3_1);
+                acc[56] += (double)v7_12_0;
+                const VT v7_13_0 = QCy * v7_5_0 + WQy * v7_5_1 + (VT)2.0 * oo2ze * v2_5_1 + (VT)1.0 * oo2e * (v7_1_0 - rho_e * v7_1_1);
+                acc[57] += (double)v7_13_0;
+                const VT v7_14_0 = QCz * v7_6_0 + WQz * v7_6_1 + (VT)1.0 * oo2e * (v7_1_0 - rho_e * v7_1_1);
+                acc[58] += (double)v7_14_0;
+                const VT v7_15_0 = QCx * v7_8_0 + WQx * v7_8_1;
+                acc[59] += (double)v7_15_0;
+                const VT v7_16_0 = QCy * v7_7_0 + WQy * v7_7_1 + (VT)2.0 * oo2ze * v2_7_1 + (VT)2.0 * oo2e * (v7_2_0 - rho_e * v7_2_1);
+                acc[60] += (double)v7_16_0;
+                const VT v7_17_0 = QCy * v7_8_0 + WQy * v7_8_1 + (VT)2.0 * oo2ze * v2_8_1 + (VT)1.0 * oo2e * (v7_3_0 - rho_e * v7_3_1);
+                acc[61] += (double)v7_17_0;
+                const VT v7_18_0 = QCz * v7_8_0 + WQz * v7_8_1 + (VT)1.0 * oo2e * (v7_2_0 - rho_e * v7_2_1);
+                acc[62] += (double)v7_18_0;
+                const VT v7_19_0 = QCz * v7_9_0 + WQz * v7_9_1 + (VT)2.0 * oo2e * (v7_3_0 - rho_e * v7_3_1);
+                acc[63] += (double)v7_19_0;
+                acc[64] += (double)v8_4_0;
+                acc[65] += (double)v8_5_0;
+                acc[66] += (double)v8_6_0;
+                acc[67] += (double)v8_7_0;
+                acc[68] += (double)v8_8_0;
+                acc[69] += (double)v8_9_0;
+                const VT v8_10_0 = QCx * v8_4_0 + WQx * v8_4_1 + (VT)2.0 * oo2e * (v8_1_0 - rho_e * v8_1_1);
+                acc[70] += (double)v8_10_0;
+                const VT v8_11_0 = QCx * v8_5_0 + WQx * v8_5_1 + (VT)1.0 * oo2e * (v8_2_0 - rho_e * v8_2_1);
+                acc[71] += (double)v8_11_0;
+                const VT v8_12_0 = QCx * v8_6_0 + WQx * v8_6_1 + (VT)1.0 * oo2e * (v8_3_0 - rho_e * v8_3_1);
+                acc[72] += (double)v8_12_0;
+                const VT v8_13_0 = QCy * v8_5_0 + WQy * v8_5_1 + (VT)1.0 * oo2ze * v3_5_1 + (VT)1.0 * oo2e * (v8_1_0 - rho_e * v8_1_1);
+                acc[73] += (double)v8_13_0;
+                const VT v8_14_0 = QCz * v8_6_0 + WQz * v8_6_1 + (VT)1.0 * oo2ze * v2_6_1 + (VT)1.0 * oo2e * (v8_1_0 - rho_e * v8_1_1);
+                acc[74] += (double)v8_14_0;
+                const VT v8_15_0 = QCx * v8_8_0 + WQx * v8_8_1;
+                acc[75] += (double)v8_15_0;
+                const VT v8_16_0 = QCy * v8_7_0 + WQy * v8_7_1 + (VT)1.0 * oo2ze * v3_7_1 + (VT)2.0 * oo2e * (v8_2_0 - rho_e * v8_2_1);
+                acc[76] += (double)v8_16_0;
+                const VT v8_17_0 = QCy * v8_8_0 + WQy * v8_8_1 + (VT)1.0 * oo2ze * v3_8_1 + (VT)1.0 * oo2e * (v8_3_0 - rho_e * v8_3_1);
+                acc[77] += (double)v8_17_0;
+                const VT v8_18_0 = QCz * v8_8_0 + WQz * v8_8_1 + (VT)1.0 * oo2ze * v2_8_1 + (VT)1.0 * oo2e * (v8_2_0 - rho_e * v8_2_1);
+                acc[78] += (double)v8_18_0;
+                const VT v8_19_0 = QCz * v8_9_0 + WQz * v8_9_1 + (VT)1.0 * oo2ze * v2_9_1 + (VT)2.0 * oo2e * (v8_3_0 - rho_e * v8_3_1);
+                acc[79] += (double)v8_19_0;
+                acc[80] += (double)v9_4_0;
+                acc[81] += (double)v9_5_0;
+                acc[82] += (double)v9_6_0;
+                acc[83] += (double)v9_7_0;
+                acc[84] += (double)v9_8_0;
+                acc[85] += (double)v9_9_0;
+                const VT v9_10_0 = QCx * v9_4_0 + WQx * v9_4_1 + (VT)2.0 * oo2e * (v9_1_0 - rho_e * v9_1_1);
+                acc[86] += (double)v9_10_0;
+                const VT v9_11_0 = QCx * v9_5_0 + WQx * v9_5_1 + (VT)1.0 * oo2e * (v9_2_0 - rho_e * v9_2_1);
+                acc[87] += (double)v9_11_0;
+                const VT v9_12_0 = QCx * v9_6_0 + WQx * v9_6_1 + (VT)1.0 * oo2e * (v9_3_0 - rho_e * v9_3_1);
+                acc[88] += (double)v9_12_0;
+                const VT v9_13_0 = QCy * v9_5_0 + WQy * v9_5_1 + (VT)1.0 * oo2e * (v9_1_0 - rho_e * v9_1_1);
+                acc[89] += (double)v9_13_0;
+                const VT v9_14_0 = QCz * v9_6_0 + WQz * v9_6_1 + (VT)2.0 * oo2ze * v3_6_1 + (VT)1.0 * oo2e * (v9_1_0 - rho_e * v9_1_1);
+                acc[90] += (double)v9_14_0;
+                const VT v9_15_0 = QCx * v9_8_0 + WQx * v9_8_1;
+                acc[91] += (double)v9_15_0;
+                const VT v9_16_0 = QCy * v9_7_0 + WQy * v9_7_1 + (VT)2.0 * oo2e * (v9_2_0 - rho_e * v9_2_1);
+                acc[92] += (double)v9_16_0;
+                const VT v9_17_0 = QCy * v9_8_0 + WQy * v9_8_1 + (VT)1.0 * oo2e * (v9_3_0 - rho_e * v9_3_1);
+                acc[93] += (double)v9_17_0;
+                const VT v9_18_0 = QCz * v9_8_0 + WQz * v9_8_1 + (VT)2.0 * oo2ze * v3_8_1 + (VT)1.0 * oo2e * (v9_2_0 - rho_e * v9_2_1);
+                acc[94] += (double)v9_18_0;
+                const VT v9_19_0 = QCz * v9_9_0 + WQz * v9_9_1 + (VT)2.0 * oo2ze * v3_9_1 + (VT)2.0 * oo2e * (v9_3_0 - rho_e * v9_3_1);
+                acc[95] += (double)v9_19_0;
+                acc[96] += (double)v10_4_0;
+                acc[97] += (double)v10_5_0;
+                acc[98] += (double)v10_6_0;
+                acc[99] += (double)v10_7_0;
+                acc[100] += (double)v10_8_0;
+                acc[101] += (double)v10_9_0;
+                const VT v10_10_0 = QCx * v10_4_0 + WQx * v10_4_1 + (VT)3.0 * oo2ze * v4_4_1 + (VT)2.0 * oo2e * (v10_1_0 - rho_e * v10_1_1);
+                acc[102] += (double)v10_10_0;
+                const VT v10_11_0 = QCx * v10_5_0 + WQx * v10_5_1 + (VT)3.0 * oo2ze * v4_5_1 + (VT)1.0 * oo2e * (v10_2_0 - rho_e * v10_2_1);
+                acc[103] += (double)v10_11_0;
+                const VT v10_12_0 = QCx * v10_6_0 + WQx * v10_6_1 + (VT)3.0 * oo2ze * v4_6_1 + (VT)1.0 * oo2e * (v10_3_0 - rho_e * v10_3_1);
+                acc[104] += (double)v10_12_0;
+                const VT v10_13_0 = QCy * v10_5_0 + WQy * v10_5_1 + (VT)1.0 * oo2e * (v10_1_0 - rho_e * v10_1_1);
+                acc[105] += (double)v10_13_0;
+                const VT v10_14_0 = QCz * v10_6_0 + WQz * v10_6_1 + (VT)1.0 * oo2e * (v10_1_0 - rho_e * v10_1_1);
+                acc[106] += (double)v10_14_0;
+                const VT v10_15_0 = QCx * v10_8_0 + WQx * v10_8_1 + (VT)3.0 * oo2ze * v4_8_1;
+                acc[107] += (double)v10_15_0;
+                const VT v10_16_0 = QCy * v10_7_0 + WQy * v10_7_1 + (VT)2.0 * oo2e * (v10_2_0 - rho_e * v10_2_1);
+                acc[108] += (double)v10_16_0;
+                const VT v10_17_0 = QCy * v10_8_0 + WQy * v10_8_1 + (VT)1.0 * oo2e * (v10_3_0 - rho_e * v10_3_1);
+                acc[109] += (double)v10_17_0;
+                const VT v10_18_0 = QCz * v10_8_0 + WQz * v10_8_1 + (VT)1.0 * oo2e * (v10_2_0 - rho_e * v10_2_1);
+                acc[110] += (double)v10_18_0;
+                const VT v10_19_0 = QCz * v10_9_0 + WQz * v10_9_1 + (VT)2.0 * oo2e * (v10_3_0 - rho_e * v10_3_1);
+                acc[111] += (double)v10_19_0;
+                acc[112] += (double)v11_4_0;
+                acc[113] += (double)v11_5_0;
+                acc[114] += (double)v11_6_0;
+                acc[115] += (double)v11_7_0;
+                acc[116] += (double)v11_8_0;
+                acc[117] += (double)v11_9_0;
+                const VT v11_10_0 = QCx * v11_4_0 + WQx * v11_4_1 + (VT)2.0 * oo2ze * v5_4_1 + (VT)2.0 * oo2e * (v11_1_0 - rho_e * v11_1_1);
+                acc[118] += (double)v11_10_0;
+                const VT v11_11_0 = QCx * v11_5_0 + WQx * v11_5_1 + (VT)2.0 * oo2ze * v5_5_1 + (VT)1.0 * oo2e * (v11_2_0 - rho_e * v11_2_1);
+                acc[119] += (double)v11_11_0;
+                const VT v11_12_0 = QCx * v11_6_0 + WQx * v11_6_1 + (VT)2.0 * oo2ze * v5_6_1 + (VT)1.0 * oo2e * (v11_3_0 - rho_e * v11_3_1);
+                acc[120] += (double)v11_12_0;
+                const VT v11_13_0 = QCy * v11_5_0 + WQy * v11_5_1 + (VT)1.0 * oo2ze * v4_5_1 + (VT)1.0 * oo2e * (v11_1_0 - rho_e * v11_1_1);
+                acc[121] += (double)v11_13_0;
+                const VT v11_14_0 = QCz * v11_6_0 + WQz * v11_6_1 + (VT)1.0 * oo2e * (v11_1_0 - rho_e * v11_1_1);
+                acc[122] += (double)v11_14_0;
+                const VT v11_15_0 = QCx * v11_8_0 + WQx * v11_8_1 + (VT)2.0 * oo2ze * v5_8_1;
+                acc[123] += (double)v11_15_0;
+                const VT v11_16_0 = QCy * v11_7_0 + WQy * v11_7_1 + (VT)1.0 * oo2ze * v4_7_1 + (VT)2.0 * oo2e * (v11_2_0 - rho_e * v11_2_1);
+                acc[124] += (double)v11_16_0;
+                const VT v11_17_0 = QCy * v11_8_0 + WQy * v11_8_1 + (VT)1.0 * oo2ze * v4_8_1 + (VT)1.0 * oo2e * (v11_3_0 - rho_e * v11_3_1);
+                acc[125] += (double)v11_17_0;
+                const VT v11_18_0 = QCz * v11_8_0 + WQz * v11_8_1 + (VT)1.0 * oo2e * (v11_2_0 - rho_e * v11_2_1);
+                acc[126] += (double)v11_18_0;
+                const VT v11_19_0 = QCz * v11_9_0 + WQz * v11_9_1 + (VT)2.0 * oo2e * (v11_3_0 - rho_e * v11_3_1);
+                acc[127] += (double)v11_19_0;
+                acc[128] += (double)v12_4_0;
+                acc[129] += (double)v12_5_0;
+                acc[130] += (double)v12_6_0;
+                acc[131] += (double)v12_7_0;
+                acc[132] += (double)v12_8_0;
+                acc[133] += (double)v12_9_0;
+                const VT v12_10_0 = QCx * v12_4_0 + WQx * v12_4_1 + (VT)2.0 * oo2ze * v6_4_1 + (VT)2.0 * oo2e * (v12_1_0 - rho_e * v12_1_1);
+                acc[134] += (double)v12_10_0;
+                const VT v12_11_0 = QCx * v12_5_0 + WQx * v12_5_1 + (VT)2.0 * oo2ze * v6_5_1 + (VT)1.0 * oo2e * (v12_2_0 - rho_e * v12_2_1);
+                acc[135] += (double)v12_11_0;
+                const VT v12_12_0 = QCx * v12_6_0 + WQx * v12_6_1 + (VT)2.0 * oo2ze * v6_6_1 + (VT)1.0 * oo2e * (v12_3_0 - rho_e * v12_3_1);
+                acc[136] += (double)v12_12_0;
+                const VT v12_13_0 = QCy * v12_5_0 + WQy * v12_5_1 + (VT)1.0 * oo2e * (v12_1_0 - rho_e * v12_1_1);
+                acc[137] += (double)v12_13_0;
+                const VT v12_14_0 = QCz * v12_6_0 + WQz * v12_6_1 + (VT)1.0 * oo2ze * v4_6_1 + (VT)1.0 * oo2e * (v12_1_0 - rho_e * v12_1_1);
+                acc[138] += (double)v12_14_0;
+                const VT v12_15_0 = QCx * v12_8_0 + WQx * v12_8_1 + (VT)2.0 * oo2ze * v6_8_1;
+                acc[139] += (double)v12_15_0;
+                const VT v12_16_0 = QCy * v12_7_0 + WQy * v12_7_1 + (VT)2.0 * oo2e * (v12_2_0 - rho_e * v12_2_1);
+                acc[140] += (double)v12_16_0;
+                const VT v12_17_0 = QCy * v12_8_0 + WQy * v12_8_1 + (VT)1.0 * oo2e * (v12_3_0 - rho_e * v12_3_1);
+                acc[141] += (double)v12_17_0;
+                const VT v12_18_0 = QCz * v12_8_0 + WQz * v12_8_1 + (VT)1.0 * oo2ze * v4_8_1 + (VT)1.0 * oo2e * (v12_2_0 - rho_e * v12_2_1);
+                acc[142] += (double)v12_18_0;
+                const VT v12_19_0 = QCz * v12_9_0 + WQz * v12_9_1 + (VT)1.0 * oo2ze * v4_9_1 + (VT)2.0 * oo2e * (v12_3_0 - rho_e * v12_3_1);
+                acc[143] += (double)v12_19_0;
+                acc[144] += (double)v13_4_0;
+                acc[145] += (double)v13_5_0;
+                acc[146] += (double)v13_6_0;
+                acc[147] += (double)v13_7_0;
+                acc[148] += (double)v13_8_0;
+                acc[149] += (double)v13_9_0;
+                const VT v13_10_0 = QCx * v13_4_0 + WQx * v13_4_1 + (VT)1.0 * oo2ze * v7_4_1 + (VT)2.0 * oo2e * (v13_1_0 - rho_e * v13_1_1);
+                acc[150] += (double)v13_10_0;
+                const VT v13_11_0 = QCx * v13_5_0 + WQx * v13_5_1 + (VT)1.0 * oo2ze * v7_5_1 + (VT)1.0 * oo2e * (v13_2_0 - rho_e * v13_2_1);
+                acc[151] += (double)v13_11_0;
+                const VT v13_12_0 = QCx * v13_6_0 + WQx * v13_6_1 + (VT)1.0 * oo2ze * v7_6_1 + (VT)1.0 * oo2e * (v13_3_0 - rho_e * v13_3_1);
+                acc[152] += (double)v13_12_0;
+                const VT v13_13_0 = QCy * v13_5_0 + WQy * v13_5_1 + (VT)2.0 * oo2ze * v5_5_1 + (VT)1.0 * oo2e * (v13_1_0 - rho_e * v13_1_1);
+                acc[153] += (double)v13_13_0;
+                const VT v13_14_0 = QCz * v13_6_0 + WQz * v13_6_1 + (VT)1.0 * oo2e * (v13_1_0 - rho_e * v13_1_1);
+                acc[154] += (double)v13_14_0;
+                const VT v13_15_0 = QCx * v13_8_0 + WQx * v13_8_1 + (VT)1.0 * oo2ze * v7_8_1;
+                acc[155] += (double)v13_15_0;
+                const VT v13_16_0 = QCy * v13_7_0 + WQy * v13_7_1 + (VT)2.0 * oo2ze * v5_7_1 + (VT)2.0 * oo2e * (v13_2_0 - rho_e * v13_2_1);
+                acc[156] += (double)v13_16_0;
+                const VT v13_17_0 = QCy * v13_8_0 + WQy * v13_8_1 + (VT)2.0 * oo2ze * v5_8_1 + (VT)1.0 * oo2e * (v13_3_0 - rho_e * v13_3_1);
+                acc[157] += (double)v13_17_0;
+                const VT v13_18_0 = QCz * v13_8_0 + WQz * v13_8_1 + (VT)1.0 * oo2e * (v13_2_0 - rho_e * v13_2_1);
+                acc[158] += (double)v13_18_0;
+                const VT v13_19_0 = QCz * v13_9_0 + WQz * v13_9_1 + (VT)2.0 * oo2e * (v13_3_0 - rho_e * v13_3_1);
+                acc[159] += (double)v13_19_0;
+                acc[160] += (double)v14_4_0;
+                acc[161] += (double)v14_5_0;
+                acc[162] += (double)v14_6_0;
+                acc[163] += (double)v14_7_0;
+                acc[164] += (double)v14_8_0;
+                acc[165] += (double)v14_9_0;
+                const VT v14_10_0 = QCx * v14_4_0 + WQx * v14_4_1 + (VT)1.0 * oo2ze * v9_4_1 + (VT)2.0 * oo2e * (v14_1_0 - rho_e * v14_1_1);
+                acc[166] += (double)v14_10_0;
+                const VT v14_11_0 = QCx * v14_5_0 + WQx * v14_5_1 + (VT)1.0 * oo2ze * v9_5_1 + (VT)1.0 * oo2e * (v14_2_0 - rho_e * v14_2_1);
+                acc[167] += (double)v14_11_0;
+                const VT v14_12_0 = QCx * v14_6_0 + WQx * v14_6_1 + (VT)1.0 * oo2ze * v9_6_1 + (VT)1.0 * oo2e * (v14_3_0 - rho_e * v14_3_1);
+                acc[168] += (double)v14_12_0;
+                const VT v14_13_0 = QCy * v14_5_0 + WQy * v14_5_1 + (VT)1.0 * oo2e * (v14_1_0 - rho_e * v14_1_1);
+                acc[169] += (double)v14_13_0;
+                const VT v14_14_0 = QCz * v14_6_0 + WQz * v14_6_1 + (VT)2.0 * oo2ze * v6_6_1 + (VT)1.0 * oo2e * (v14_1_0 - rho_e * v14_1_1);
+                acc[170] += (double)v14_14_0;
+                const VT v14_15_0 = QCx * v14_8_0 + WQx * v14_8_1 + (VT)1.0 * oo2ze * v9_8_1;
+                acc[171] += (double)v14_15_0;
+                const VT v14_16_0 = QCy * v14_7_0 + WQy * v14_7_1 + (VT)2.0 * oo2e * (v14_2_0 - rho_e * v14_2_1);
+                acc[172] += (double)v14_16_0;
+                const VT v14_17_0 = QCy * v14_8_0 + WQy * v14_8_1 + (VT)1.0 * oo2e * (v14_3_0 - rho_e * v14_3_1);
+                acc[173] += (double)v14_17_0;
+                const VT v14_18_0 = QCz * v14_8_0 + WQz * v14_8_1 + (VT)2.0 * oo2ze * v6_8_1 + (VT)1.0 * oo2e * (v14_2_0 - rho_e * v14_2_1);
+                acc[174] += (double)v14_18_0;
+                const VT v14_19_0 = QCz * v14_9_0 + WQz * v14_9_1 + (VT)2.0 * oo2ze * v6_9_1 + (VT)2.0 * oo2e * (v14_3_0 - rho_e * v14_3_1);
+                acc[175] += (double)v14_19_0;
+                acc[176] += (double)v15_4_0;
+                acc[177] += (double)v15_5_0;
+                acc[178] += (double)v15_6_0;
+                acc[179] += (double)v15_7_0;
+                acc[180] += (double)v15_8_0;
+                acc[181] += (double)v15_9_0;
+                const VT v15_10_0 = QCx * v15_4_0 + WQx * v15_4_1 + (VT)1.0 * oo2ze * v8_4_1 + (VT)2.0 * oo2e * (v15_1_0 - rho_e * v15_1_1);
+                acc[182] += (double)v15_10_0;
+                const VT v15_11_0 = QCx * v15_5_0 + WQx * v15_5_1 + (VT)1.0 * oo2ze * v8_5_1 + (VT)1.0 * oo2e * (v15_2_0 - rho_e * v15_2_1);
+                acc[183] += (double)v15_11_0;
+                const VT v15_12_0 = QCx * v15_6_0 + WQx * v15_6_1 + (VT)1.0 * oo2ze * v8_6_1 + (VT)1.0 * oo2e * (v15_3_0 - rho_e * v15_3_1);
+                acc[184] += (double)v15_12_0;
+                const VT v15_13_0 = QCy * v15_5_0 + WQy * v15_5_1 + (VT)1.0 * oo2ze * v6_5_1 + (VT)1.0 * oo2e * (v15_1_0 - rho_e * v15_1_1);
+                acc[185] += (double)v15_13_0;
+                const VT v15_14_0 = QCz * v15_6_0 + WQz * v15_6_1 + (VT)1.0 * oo2ze * v5_6_1 + (VT)1.0 * oo2e * (v15_1_0 - rho_e * v15_1_1);
+                acc[186] += (double)v15_14_0;
+                const VT v15_15_0 = QCx * v15_8_0 + WQx * v15_8_1 + (VT)1.0 * oo2ze * v8_8_1;
+                acc[187] += (double)v15_15_0;
+                const VT v15_16_0 = QCy * v15_7_0 + WQy * v15_7_1 + (VT)1.0 * oo2ze * v6_7_1 + (VT)2.0 * oo2e * (v15_2_0 - rho_e * v15_2_1);
+                acc[188] += (double)v15_16_0;
+                const VT v15_17_0 = QCy * v15_8_0 + WQy * v15_8_1 + (VT)1.0 * oo2ze * v6_8_1 + (VT)1.0 * oo2e * (v15_3_0 - rho_e * v15_3_1);
+                acc[189] += (double)v15_17_0;
+                const VT v15_18_0 = QCz * v15_8_0 + WQz * v15_8_1 + (VT)1.0 * oo2ze * v5_8_1 + (VT)1.0 * oo2e * (v15_2_0 - rho_e * v15_2_1);
+                acc[190] += (double)v15_18_0;
+                const VT v15_19_0 = QCz * v15_9_0 + WQz * v15_9_1 + (VT)1.0 * oo2ze * v5_9_1 + (VT)2.0 * oo2e * (v15_3_0 - rho_e * v15_3_1);
+                acc[191] += (double)v15_19_0;
+                acc[192] += (double)v16_4_0;
+                acc[193] += (double)v16_5_0;
+                acc[194] += (double)v16_6_0;
+                acc[195] += (double)v16_7_0;
+                acc[196] += (double)v16_8_0;
+                acc[197] += (double)v16_9_0;
+                const VT v16_10_0 = QCx * v16_4_0 + WQx * v16_4_1 + (VT)2.0 * oo2e * (v16_1_0 - rho_e * v16_1_1);
+                acc[198] += (double)v16_10_0;
+                const VT v16_11_0 = QCx * v16_5_0 + WQx * v16_5_1 + (VT)1.0 * oo2e * (v16_2_0 - rho_e * v16_2_1);
+                acc[199] += (double)v16_11_0;
+                const VT v16_12_0 = QCx * v16_6_0 + WQx * v16_6_1 + (VT)1.0 * oo2e * (v16_3_0 - rho_e * v16_3_1);
+                acc[200] += (double)v16_12_0;
+                const VT v16_13_0 = QCy * v16_5_0 + WQy * v16_5_1 + (VT)3.0 * oo2ze * v7_5_1 + (VT)1.0 * oo2e * (v16_1_0 - rho_e * v16_1_1);
+                acc[201] += (double)v16_13_0;
+                const VT v16_14_0 = QCz * v16_6_0 + WQz * v16_6_1 + (VT)1.0 * oo2e * (v16_1_0 - rho_e * v16_1_1);
+                acc[202] += (double)v16_14_0;
+                const VT v16_15_0 = QCx * v16_8_0 + WQx * v16_8_1;
+                acc[203] += (double)v16_15_0;
+                const VT v16_16_0 = QCy * v16_7_0 + WQy * v16_7_1 + (VT)3.0 * oo2ze * v7_7_1 + (VT)2.0 * oo2e * (v16_2_0 - rho_e * v16_2_1);
+                acc[204] += (double)v16_16_0;
+                const VT v16_17_0 = QCy * v16_8_0 + WQy * v16_8_1 + (VT)3.0 * oo2ze * v7_8_1 + (VT)1.0 * oo2e * (v16_3_0 - rho_e * v16_3_1);
+                acc[205] += (double)v16_17_0;
+                const VT v16_18_0 = QCz * v16_8_0 + WQz * v16_8_1 + (VT)1.0 * oo2e * (v16_2_0 - rho_e * v16_2_1);
+                acc[206] += (double)v16_18_0;
+                const VT v16_19_0 = QCz * v16_9_0 + WQz * v16_9_1 + (VT)2.0 * oo2e * (v16_3_0 - rho_e * v16_3_1);
+                acc[207] += (double)v16_19_0;
+                acc[208] += (double)v17_4_0;
+                acc[209] += (double)v17_5_0;
+                acc[210] += (double)v17_6_0;
+                acc[211] += (double)v17_7_0;
+                acc[212] += (double)v17_8_0;
+                acc[213] += (double)v17_9_0;
+                const VT v17_10_0 = QCx * v17_4_0 + WQx * v17_4_1 + (VT)2.0 * oo2e * (v17_1_0 - rho_e * v17_1_1);
+                acc[214] += (double)v17_10_0;
+                const VT v17_11_0 = QCx * v17_5_0 + WQx * v17_5_1 + (VT)1.0 * oo2e * (v17_2_0 - rho_e * v17_2_1);
+                acc[215] += (double)v17_11_0;
+                const VT v17_12_0 = QCx * v17_6_0 + WQx * v17_6_1 + (VT)1.0 * oo2e * (v17_3_0 - rho_e * v17_3_1);
+                acc[216] += (double)v17_12_0;
+                const VT v17_13_0 = QCy * v17_5_0 + WQy * v17_5_1 + (VT)2.0 * oo2ze * v8_5_1 + (VT)1.0 * oo2e * (v17_1_0 - rho_e * v17_1_1);
+                acc[217] += (double)v17_13_0;
+                const VT v17_14_0 = QCz * v17_6_0 + WQz * v17_6_1 + (VT)1.0 * oo2ze * v7_6_1 + (VT)1.0 * oo2e * (v17_1_0 - rho_e * v17_1_1);
+                acc[218] += (double)v17_14_0;
+                const VT v17_15_0 = QCx * v17_8_0 + WQx * v17_8_1;
+                acc[219] += (double)v17_15_0;
+                const VT v17_16_0 = QCy * v17_7_0 + WQy * v17_7_1 + (VT)2.0 * oo2ze * v8_7_1 + (VT)2.0 * oo2e * (v17_2_0 - rho_e * v17_2_1);
+                acc[220] += (double)v17_16_0;
+                const VT v17_17_0 = QCy * v17_8_0 + WQy * v17_8_1 + (VT)2.0 * oo2ze * v8_8_1 + (VT)1.0 * oo2e * (v17_3_0 - rho_e * v17_3_1);
+                acc[221] += (double)v17_17_0;
+                const VT v17_18_0 = QCz * v17_8_0 + WQz * v17_8_1 + (VT)1.0 * oo2ze * v7_8_1 + (VT)1.0 * oo2e * (v17_2_0 - rho_e * v17_2_1);
+                acc[222] += (double)v17_18_0;
+                const VT v17_19_0 = QCz * v17_9_0 + WQz * v17_9_1 + (VT)1.0 * oo2ze * v7_9_1 + (VT)2.0 * oo2e * (v17_3_0 - rho_e * v17_3_1);
+                acc[223] += (double)v17_19_0;
+                acc[224] += (double)v18_4_0;
+                acc[225] += (double)v18_5_0;
+                acc[226] += (double)v18_6_0;
+                acc[227] += (double)v18_7_0;
+                acc[228] += (double)v18_8_0;
+                acc[229] += (double)v18_9_0;
+                const VT v18_10_0 = QCx * v18_4_0 + WQx * v18_4_1 + (VT)2.0 * oo2e * (v18_1_0 - rho_e * v18_1_1);
+                acc[230] += (double)v18_10_0;
+                const VT v18_11_0 = QCx * v18_5_0 + WQx * v18_5_1 + (VT)1.0 * oo2e * (v18_2_0 - rho_e * v18_2_1);
+                acc[231] += (double)v18_11_0;
+                const VT v18_12_0 = QCx * v18_6_0 + WQx * v18_6_1 + (VT)1.0 * oo2e * (v18_3_0 - rho_e * v18_3_1);
+                acc[232] += (double)v18_12_0;
+                const VT v18_13_0 = QCy * v18_5_0 + WQy * v18_5_1 + (VT)1.0 * oo2ze * v9_5_1 + (VT)1.0 * oo2e * (v18_1_0 - rho_e * v18_1_1);
+                acc[233] += (double)v18_13_0;
+                const VT v18_14_0 = QCz * v18_6_0 + WQz * v18_6_1 + (VT)2.0 * oo2ze * v8_6_1 + (VT)1.0 * oo2e * (v18_1_0 - rho_e * v18_1_1);
+                acc[234] += (double)v18_14_0;
+                const VT v18_15_0 = QCx * v18_8_0 + WQx * v18_8_1;
+                acc[235] += (double)v18_15_0;
+                const VT v18_16_0 = QCy * v18_7_0 + WQy * v18_7_1 + (VT)1.0 * oo2ze * v9_7_1 + (VT)2.0 * oo2e * (v18_2_0 - rho_e * v18_2_1);
+                acc[236] += (double)v18_16_0;
+                const VT v18_17_0 = QCy * v18_8_0 + WQy * v18_8_1 + (VT)1.0 * oo2ze * v9_8_1 + (VT)1.0 * oo2e * (v18_3_0 - rho_e * v18_3_1);
+                acc[237] += (double)v18_17_0;
+                const VT v18_18_0 = QCz * v18_8_0 + WQz * v18_8_1 + (VT)2.0 * oo2ze * v8_8_1 + (VT)1.0 * oo2e * (v18_2_0 - rho_e * v18_2_1);
+                acc[238] += (double)v18_18_0;
+                const VT v18_19_0 = QCz * v18_9_0 + WQz * v18_9_1 + (VT)2.0 * oo2ze * v8_9_1 + (VT)2.0 * oo2e * (v18_3_0 - rho_e * v18_3_1);
+                acc[239] += (double)v18_19_0;
+                acc[240] += (double)v19_4_0;
+                acc[241] += (double)v19_5_0;
+                acc[242] += (double)v19_6_0;
+                acc[243] += (double)v19_7_0;
+                acc[244] += (double)v19_8_0;
+                acc[245] += (double)v19_9_0;
+                const VT v19_10_0 = QCx * v19_4_0 + WQx * v19_4_1 + (VT)2.0 * oo2e * (v19_1_0 - rho_e * v19_1_1);
+                acc[246] += (double)v19_10_0;
+                const VT v19_11_0 = QCx * v19_5_0 + WQx * v19_5_1 + (VT)1.0 * oo2e * (v19_2_0 - rho_e * v19_2_1);
+                acc[247] += (double)v19_11_0;
+                const VT v19_12_0 = QCx * v19_6_0 + WQx * v19_6_1 + (VT)1.0 * oo2e * (v19_3_0 - rho_e * v19_3_1);
+                acc[248] += (double)v19_12_0;
+                const VT v19_13_0 = QCy * v19_5_0 + WQy * v19_5_1 + (VT)1.0 * oo2e * (v19_1_0 - rho_e * v19_1_1);
+                acc[249] += (double)v19_13_0;
+                const VT v19_14_0 = QCz * v19_6_0 + WQz * v19_6_1 + (VT)3.0 * oo2ze * v9_6_1 + (VT)1.0 * oo2e * (v19_1_0 - rho_e * v19_1_1);
+                acc[250] += (double)v19_14_0;
+                const VT v19_15_0 = QCx * v19_8_0 + WQx * v19_8_1;
+                acc[251] += (double)v19_15_0;
+                const VT v19_16_0 = QCy * v19_7_0 + WQy * v19_7_1 + (VT)2.0 * oo2e * (v19_2_0 - rho_e * v19_2_1);
+                acc[252] += (double)v19_16_0;
+                const VT v19_17_0 = QCy * v19_8_0 + WQy * v19_8_1 + (VT)1.0 * oo2e * (v19_3_0 - rho_e * v19_3_1);
+                acc[253] += (double)v19_17_0;
+                const VT v19_18_0 = QCz * v19_8_0 + WQz * v19_8_1 + (VT)3.0 * oo2ze * v9_8_1 + (VT)1.0 * oo2e * (v19_2_0 - rho_e * v19_2_1);
+                acc[254] += (double)v19_18_0;
+                const VT v19_19_0 = QCz * v19_9_0 + WQz * v19_9_1 + (VT)3.0 * oo2ze * v9_9_1 + (VT)2.0 * oo2e * (v19_3_0 - rho_e * v19_3_1);
+                acc[255] += (double)v19_19_0;
+                acc[256] += (double)v20_4_0;
+                acc[257] += (double)v20_5_0;
+                acc[258] += (double)v20_6_0;
+                acc[259] += (double)v20_7_0;
+                acc[260] += (double)v20_8_0;
+                acc[261] += (double)v20_9_0;
+                const VT v20_10_0 = QCx * v20_4_0 + WQx * v20_4_1 + (VT)4.0 * oo2ze * v10_4_1 + (VT)2.0 * oo2e * (v20_1_0 - rho_e * v20_1_1);
+                acc[262] += (double)v20_10_0;
+                const VT v20_11_0 = QCx * v20_5_0 + WQx * v20_5_1 + (VT)4.0 * oo2ze * v10_5_1 + (VT)1.0 * oo2e * (v20_2_0 - rho_e * v20_2_1);
+                acc[263] += (double)v20_11_0;
+                const VT v20_12_0 = QCx * v20_6_0 + WQx * v20_6_1 + (VT)4.0 * oo2ze * v10_6_1 + (VT)1.0 * oo2e * (v20_3_0 - rho_e * v20_3_1);
+                acc[264] += (double)v20_12_0;
+                const VT v20_13_0 = QCy * v20_5_0 + WQy * v20_5_1 + (VT)1.0 * oo2e * (v20_1_0 - rho_e * v20_1_1);
+                acc[265] += (double)v20_13_0;
+                const VT v20_14_0 = QCz * v20_6_0 + WQz * v20_6_1 + (VT)1.0 * oo2e * (v20_1_0 - rho_e * v20_1_1);
+                acc[266] += (double)v20_14_0;
+                const VT v20_15_0 = QCx * v20_8_0 + WQx * v20_8_1 + (VT)4.0 * oo2ze * v10_8_1;
+                acc[267] += (double)v20_15_0;
+                const VT v20_16_0 = QCy * v20_7_0 + WQy * v20_7_1 + (VT)2.0 * oo2e * (v20_2_0 - rho_e * v20_2_1);
+                acc[268] += (double)v20_16_0;
+                const VT v20_17_0 = QCy * v20_8_0 + WQy * v20_8_1 + (VT)1.0 * oo2e * (v20_3_0 - rho_e * v20_3_1);
+                acc[269] += (double)v20_17_0;
+                const VT v20_18_0 = QCz * v20_8_0 + WQz * v20_8_1 + (VT)1.0 * oo2e * (v20_2_0 - rho_e * v20_2_1);
+                acc[270] += (double)v20_18_0;
+                const VT v20_19_0 = QCz * v20_9_0 + WQz * v20_9_1 + (VT)2.0 * oo2e * (v20_3_0 - rho_e * v20_3_1);
+                acc[271] += (double)v20_19_0;
+                acc[272] += (double)v21_4_0;
+                acc[273] += (double)v21_5_0;
+                acc[274] += (double)v21_6_0;
+                acc[275] += (double)v21_7_0;
+                acc[276] += (double)v21_8_0;
+                acc[277] += (double)v21_9_0;
+                const VT v21_10_0 = QCx * v21_4_0 + WQx * v21_4_1 + (VT)3.0 * oo2ze * v11_4_1 + (VT)2.0 * oo2e * (v21_1_0 - rho_e * v21_1_1);
+                acc[278] += (double)v21_10_0;
+                const VT v21_11_0 = QCx * v21_5_0 + WQx * v21_5_1 + (VT)3.0 * oo2ze * v11_5_1 + (VT)1.0 * oo2e * (v21_2_0 - rho_e * v21_2_1);
+                acc[279] += (double)v21_11_0;
+                const VT v21_12_0 = QCx * v21_6_0 + WQx * v21_6_1 + (VT)3.0 * oo2ze * v11_6_1 + (VT)1.0 * oo2e * (v21_3_0 - rho_e * v21_3_1);
+                acc[280] += (double)v21_12_0;
+                const VT v21_13_0 = QCy * v21_5_0 + WQy * v21_5_1 + (VT)1.0 * oo2ze * v10_5_1 + (VT)1.0 * oo2e * (v21_1_0 - rho_e * v21_1_1);
+                acc[281] += (double)v21_13_0;
+                const VT v21_14_0 = QCz * v21_6_0 + WQz * v21_6_1 + (VT)1.0 * oo2e * (v21_1_0 - rho_e * v21_1_1);
+                acc[282] += (double)v21_14_0;
+                const VT v21_15_0 = QCx * v21_8_0 + WQx * v21_8_1 + (VT)3.0 * oo2ze * v11_8_1;
+                acc[283] += (double)v21_15_0;
+                const VT v21_16_0 = QCy * v21_7_0 + WQy * v21_7_1 + (VT)1.0 * oo2ze * v10_7_1 + (VT)2.0 * oo2e * (v21_2_0 - rho_e * v21_2_1);
+                acc[284] += (double)v21_16_0;
+                const VT v21_17_0 = QCy * v21_8_0 + WQy * v21_8_1 + (VT)1.0 * oo2ze * v10_8_1 + (VT)1.0 * oo2e * (v21_3_0 - rho_e * v21_3_1);
+                acc[285] += (double)v21_17_0;
+                const VT v21_18_0 = QCz * v21_8_0 + WQz * v21_8_1 + (VT)1.0 * oo2e * (v21_2_0 - rho_e * v21_2_1);
+                acc[286] += (double)v21_18_0;
+                const VT v21_19_0 = QCz * v21_9_0 + WQz * v21_9_1 + (VT)2.0 * oo2e * (v21_3_0 - rho_e * v21_3_1);
+                acc[287] += (double)v21_19_0;
+                acc[288] += (double)v22_4_0;
+                acc[289] += (double)v22_5_0;
+                acc[290] += (double)v22_6_0;
+                acc[291] += (double)v22_7_0;
+                acc[292] += (double)v22_8_0;
+                acc[293] += (double)v22_9_0;
+                const VT v22_10_0 = QCx * v22_4_0 + WQx * v22_4_1 + (VT)3.0 * oo2ze * v12_4_1 + (VT)2.0 * oo2e * (v22_1_0 - rho_e * v22_1_1);
+                acc[294] += (double)v22_10_0;
+                const VT v22_11_0 = QCx * v22_5_0 + WQx * v22_5_1 + (VT)3.0 * oo2ze * v12_5_1 + (VT)1.0 * oo2e * (v22_2_0 - rho_e * v22_2_1);
+                acc[295] += (double)v22_11_0;
+                const VT v22_12_0 = QCx * v22_6_0 + WQx * v22_6_1 + (VT)3.0 * oo2ze * v12_6_1 + (VT)1.0 * oo2e * (v22_3_0 - rho_e * v22_3_1);
+                acc[296] += (double)v22_12_0;
+                const VT v22_13_0 = QCy * v22_5_0 + WQy * v22_5_1 + (VT)1.0 * oo2e * (v22_1_0 - rho_e * v22_1_1);
+                acc[297] += (double)v22_13_0;
+                const VT v22_14_0 = QCz * v22_6_0 + WQz * v22_6_1 + (VT)1.0 * oo2ze * v10_6_1 + (VT)1.0 * oo2e * (v22_1_0 - rho_e * v22_1_1);
+                acc[298] += (double)v22_14_0;
+                const VT v22_15_0 = QCx * v22_8_0 + WQx * v22_8_1 + (VT)3.0 * oo2ze * v12_8_1;
+                acc[299] += (double)v22_15_0;
+                const VT v22_16_0 = QCy * v22_7_0 + WQy * v22_7_1 + (VT)2.0 * oo2e * (v22_2_0 - rho_e * v22_2_1);
+                acc[300] += (double)v22_16_0;
+                const VT v22_17_0 = QCy * v22_8_0 + WQy * v22_8_1 + (VT)1.0 * oo2e * (v22_3_0 - rho_e * v22_3_1);
+                acc[301] += (double)v22_17_0;
+                const VT v22_18_0 = QCz * v22_8_0 + WQz * v22_8_1 + (VT)1.0 * oo2ze * v10_8_1 + (VT)1.0 * oo2e * (v22_2_0 - rho_e * v22_2_1);
+                acc[302] += (double)v22_18_0;
+                const VT v22_19_0 = QCz * v22_9_0 + WQz * v22_9_1 + (VT)1.0 * oo2ze * v10_9_1 + (VT)2.0 * oo2e * (v22_3_0 - rho_e * v22_3_1);
+                acc[303] += (double)v22_19_0;
+                acc[304] += (double)v23_4_0;
+                acc[305] += (double)v23_5_0;
+                acc[306] += (double)v23_6_0;
+                acc[307] += (double)v23_7_0;
+                acc[308] += (double)v23_8_0;
+                acc[309] += (double)v23_9_0;
+                const VT v23_10_0 = QCx * v23_4_0 + WQx * v23_4_1 + (VT)2.0 * oo2ze * v13_4_1 + (VT)2.0 * oo2e * (v23_1_0 - rho_e * v23_1_1);
+                acc[310] += (double)v23_10_0;
+                const VT v23_11_0 = QCx * v23_5_0 + WQx * v23_5_1 + (VT)2.0 * oo2ze * v13_5_1 + (VT)1.0 * oo2e * (v23_2_0 - rho_e * v23_2_1);
+                acc[311] += (double)v23_11_0;
+                const VT v23_12_0 = QCx * v23_6_0 + WQx * v23_6_1 + (VT)2.0 * oo2ze * v13_6_1 + (VT)1.0 * oo2e * (v23_3_0 - rho_e * v23_3_1);
+                acc[312] += (double)v23_12_0;
+                const VT v23_13_0 = QCy * v23_5_0 + WQy * v23_5_1 + (VT)2.0 * oo2ze * v11_5_1 + (VT)1.0 * oo2e * (v23_1_0 - rho_e * v23_1_1);
+                acc[313] += (double)v23_13_0;
+                const VT v23_14_0 = QCz * v23_6_0 + WQz * v23_6_1 + (VT)1.0 * oo2e * (v23_1_0 - rho_e * v23_1_1);
+                acc[314] += (double)v23_14_0;
+                const VT v23_15_0 = QCx * v23_8_0 + WQx * v23_8_1 + (VT)2.0 * oo2ze * v13_8_1;
+                acc[315] += (double)v23_15_0;
+                const VT v23_16_0 = QCy * v23_7_0 + WQy * v23_7_1 + (VT)2.0 * oo2ze * v11_7_1 + (VT)2.0 * oo2e * (v23_2_0 - rho_e * v23_2_1);
+                acc[316] += (double)v23_16_0;
+                const VT v23_17_0 = QCy * v23_8_0 + WQy * v23_8_1 + (VT)2.0 * oo2ze * v11_8_1 + (VT)1.0 * oo2e * (v23_3_0 - rho_e * v23_3_1);
+                acc[317] += (double)v23_17_0;
+                const VT v23_18_0 = QCz * v23_8_0 + WQz * v23_8_1 + (VT)1.0 * oo2e * (v23_2_0 - rho_e * v23_2_1);
+                acc[318] += (double)v23_18_0;
+                const VT v23_19_0 = QCz * v23_9_0 + WQz * v23_9_1 + (VT)2.0 * oo2e * (v23_3_0 - rho_e * v23_3_1);
+                acc[319] += (double)v23_19_0;
+                acc[320] += (double)v24_4_0;
+                acc[321] += (double)v24_5_0;
+                acc[322] += (double)v24_6_0;
+                acc[323] += (double)v24_7_0;
+                acc[324] += (double)v24_8_0;
+                acc[325] += (double)v24_9_0;
+                const VT v24_10_0 = QCx * v24_4_0 + WQx * v24_4_1 + (VT)2.0 * oo2ze * v15_4_1 + (VT)2.0 * oo2e * (v24_1_0 - rho_e * v24_1_1);
+                acc[326] += (double)v24_10_0;
+                const VT v24_11_0 = QCx * v24_5_0 + WQx * v24_5_1 + (VT)2.0 * oo2ze * v15_5_1 + (VT)1.0 * oo2e * (v24_2_0 - rho_e * v24_2_1);
+                acc[327] += (double)v24_11_0;
+                const VT v24_12_0 = QCx * v24_6_0 + WQx * v24_6_1 + (VT)2.0 * oo2ze * v15_6_1 + (VT)1.0 * oo2e * (v24_3_0 - rho_e * v24_3_1);
+                acc[328] += (double)v24_12_0;
+                const VT v24_13_0 = QCy * v24_5_0 + WQy * v24_5_1 + (VT)1.0 * oo2ze * v12_5_1 + (VT)1.0 * oo2e * (v24_1_0 - rho_e * v24_1_1);
+                acc[329] += (double)v24_13_0;
+                const VT v24_14_0 = QCz * v24_6_0 + WQz * v24_6_1 + (VT)1.0 * oo2ze * v11_6_1 + (VT)1.0 * oo2e * (v24_1_0 - rho_e * v24_1_1);
+                acc[330] += (double)v24_14_0;
+                const VT v24_15_0 = QCx * v24_8_0 + WQx * v24_8_1 + (VT)2.0 * oo2ze * v15_8_1;
+                acc[331] += (double)v24_15_0;
+                const VT v24_16_0 = QCy * v24_7_0 + WQy * v24_7_1 + (VT)1.0 * oo2ze * v12_7_1 + (VT)2.0 * oo2e * (v24_2_0 - rho_e * v24_2_1);
+                acc[332] += (double)v24_16_0;
+                const VT v24_17_0 = QCy * v24_8_0 + WQy * v24_8_1 + (VT)1.0 * oo2ze * v12_8_1 + (VT)1.0 * oo2e * (v24_3_0 - rho_e * v24_3_1);
+                acc[333] += (double)v24_17_0;
+                const VT v24_18_0 = QCz * v24_8_0 + WQz * v24_8_1 + (VT)1.0 * oo2ze * v11_8_1 + (VT)1.0 * oo2e * (v24_2_0 - rho_e * v24_2_1);
+                acc[334] += (double)v24_18_0;
+                const VT v24_19_0 = QCz * v24_9_0 + WQz * v24_9_1 + (VT)1.0 * oo2ze * v11_9_1 + (VT)2.0 * oo2e * (v24_3_0 - rho_e * v24_3_1);
+                acc[335] += (double)v24_19_0;
+                acc[336] += (double)v25_4_0;
+                acc[337] += (double)v25_5_0;
+                acc[338] += (double)v25_6_0;
+                acc[339] += (double)v25_7_0;
+                acc[340] += (double)v25_8_0;
+                acc[341] += (double)v25_9_0;
+                const VT v25_10_0 = QCx * v25_4_0 + WQx * v25_4_1 + (VT)2.0 * oo2ze * v14_4_1 + (VT)2.0 * oo2e * (v25_1_0 - rho_e * v25_1_1);
+                acc[342] += (double)v25_10_0;
+                const VT v25_11_0 = QCx * v25_5_0 + WQx * v25_5_1 + (VT)2.0 * oo2ze * v14_5_1 + (VT)1.0 * oo2e * (v25_2_0 - rho_e * v25_2_1);
+                acc[343] += (double)v25_11_0;
+                const VT v25_12_0 = QCx * v25_6_0 + WQx * v25_6_1 + (VT)2.0 * oo2ze * v14_6_1 + (VT)1.0 * oo2e * (v25_3_0 - rho_e * v25_3_1);
+                acc[344] += (double)v25_12_0;
+                const VT v25_13_0 = QCy * v25_5_0 + WQy * v25_5_1 + (VT)1.0 * oo2e * (v25_1_0 - rho_e * v25_1_1);
+                acc[345] += (double)v25_13_0;
+                const VT v25_14_0 = QCz * v25_6_0 + WQz * v25_6_1 + (VT)2.0 * oo2ze * v12_6_1 + (VT)1.0 * oo2e * (v25_1_0 - rho_e * v25_1_1);
+                acc[346] += (double)v25_14_0;
+                const VT v25_15_0 = QCx * v25_8_0 + WQx * v25_8_1 + (VT)2.0 * oo2ze * v14_8_1;
+                acc[347] += (double)v25_15_0;
+                const VT v25_16_0 = QCy * v25_7_0 + WQy * v25_7_1 + (VT)2.0 * oo2e * (v25_2_0 - rho_e * v25_2_1);
+                acc[348] += (double)v25_16_0;
+                const VT v25_17_0 = QCy * v25_8_0 + WQy * v25_8_1 + (VT)1.0 * oo2e * (v25_3_0 - rho_e * v25_3_1);
+                acc[349] += (double)v25_17_0;
+                const VT v25_18_0 = QCz * v25_8_0 + WQz * v25_8_1 + (VT)2.0 * oo2ze * v12_8_1 + (VT)1.0 * oo2e * (v25_2_0 - rho_e * v25_2_1);
+                acc[350] += (double)v25_18_0;
+                const VT v25_19_0 = QCz * v25_9_0 + WQz * v25_9_1 + (VT)2.0 * oo2ze * v12_9_1 + (VT)2.0 * oo2e * (v25_3_0 - rho_e * v25_3_1);
+                acc[351] += (double)v25_19_0;
+                acc[352] += (double)v26_4_0;
+                acc[353] += (double)v26_5_0;
+                acc[354] += (double)v26_6_0;
+                acc[355] += (double)v26_7_0;
+                acc[356] += (double)v26_8_0;
+                acc[357] += (double)v26_9_0;
+                const VT v26_10_0 = QCx * v26_4_0 + WQx * v26_4_1 + (VT)1.0 * oo2ze * v16_4_1 + (VT)2.0 * oo2e * (v26_1_0 - rho_e * v26_1_1);
+                acc[358] += (double)v26_10_0;
+                const VT v26_11_0 = QCx * v26_5_0 + WQx * v26_5_1 + (VT)1.0 * oo2ze * v16_5_1 + (VT)1.0 * oo2e * (v26_2_0 - rho_e * v26_2_1);
+                acc[359] += (double)v26_11_0;
+                const VT v26_12_0 = QCx * v26_6_0 + WQx * v26_6_1 + (VT)1.0 * oo2ze * v16_6_1 + (VT)1.0 * oo2e * (v26_3_0 - rho_e * v26_3_1);
+                acc[360] += (double)v26_12_0;
+                const VT v26_13_0 = QCy * v26_5_0 + WQy * v26_5_1 + (VT)3.0 * oo2ze * v13_5_1 + (VT)1.0 * oo2e * (v26_1_0 - rho_e * v26_1_1);
+                acc[361] += (double)v26_13_0;
+                const VT v26_14_0 = QCz * v26_6_0 + WQz * v26_6_1 + (VT)1.0 * oo2e * (v26_1_0 - rho_e * v26_1_1);
+                acc[362] += (double)v26_14_0;
+                const VT v26_15_0 = QCx * v26_8_0 + WQx * v26_8_1 + (VT)1.0 * oo2ze * v16_8_1;
+                acc[363] += (double)v26_15_0;
+                const VT v26_16_0 = QCy * v26_7_0 + WQy * v26_7_1 + (VT)3.0 * oo2ze * v13_7_1 + (VT)2.0 * oo2e * (v26_2_0 - rho_e * v26_2_1);
+                acc[364] += (double)v26_16_0;
+                const VT v26_17_0 = QCy * v26_8_0 + WQy * v26_8_1 + (VT)3.0 * oo2ze * v13_8_1 + (VT)1.0 * oo2e * (v26_3_0 - rho_e * v26_3_1);
+                acc[365] += (double)v26_17_0;
+                const VT v26_18_0 = QCz * v26_8_0 + WQz * v26_8_1 + (VT)1.0 * oo2e * (v26_2_0 - rho_e * v26_2_1);
+                acc[366] += (double)v26_18_0;
+                const VT v26_19_0 = QCz * v26_9_0 + WQz * v26_9_1 + (VT)2.0 * oo2e * (v26_3_0 - rho_e * v26_3_1);
+                acc[367] += (double)v26_19_0;
+                acc[368] += (double)v27_4_0;
+                acc[369] += (double)v27_5_0;
+                acc[370] += (double)v27_6_0;
+                acc[371] += (double)v27_7_0;
+                acc[372] += (double)v27_8_0;
+                acc[373] += (double)v27_9_0;
+                const VT v27_10_0 = QCx * v27_4_0 + WQx * v27_4_1 + (VT)1.0 * oo2ze * v17_4_1 + (VT)2.0 * oo2e * (v27_1_0 - rho_e * v27_1_1);
+                acc[374] += (double)v27_10_0;
+                const VT v27_11_0 = QCx * v27_5_0 + WQx * v27_5_1 + (VT)1.0 * oo2ze * v17_5_1 + (VT)1.0 * oo2e * (v27_2_0 - rho_e * v27_2_1);
+                acc[375] += (double)v27_11_0;
+                const VT v27_12_0 = QCx * v27_6_0 + WQx * v27_6_1 + (VT)1.0 * oo2ze * v17_6_1 + (VT)1.0 * oo2e * (v27_3_0 - rho_e * v27_3_1);
+                acc[376] += (double)v27_12_0;
+                const VT v27_13_0 = QCy * v27_5_0 + WQy * v27_5_1 + (VT)2.0 * oo2ze * v15_5_1 + (VT)1.0 * oo2e * (v27_1_0 - rho_e * v27_1_1);
+                acc[377] += (double)v27_13_0;
+                const VT v27_14_0 = QCz * v27_6_0 + WQz * v27_6_1 + (VT)1.0 * oo2ze * v13_6_1 + (VT)1.0 * oo2e * (v27_1_0 - rho_e * v27_1_1);
+                acc[378] += (double)v27_14_0;
+                const VT v27_15_0 = QCx * v27_8_0 + WQx * v27_8_1 + (VT)1.0 * oo2ze * v17_8_1;
+                acc[379] += (double)v27_15_0;
+                const VT v27_16_0 = QCy * v27_7_0 + WQy * v27_7_1 + (VT)2.0 * oo2ze * v15_7_1 + (VT)2.0 * oo2e * (v27_2_0 - rho_e * v27_2_1);
+                acc[380] += (double)v27_16_0;
+                const VT v27_17_0 = QCy * v27_8_0 + WQy * v27_8_1 + (VT)2.0 * oo2ze * v15_8_1 + (VT)1.0 * oo2e * (v27_3_0 - rho_e * v27_3_1);
+                acc[381] += (double)v27_17_0;
+                const VT v27_18_0 = QCz * v27_8_0 + WQz * v27_8_1 + (VT)1.0 * oo2ze * v13_8_1 + (VT)1.0 * oo2e * (v27_2_0 - rho_e * v27_2_1);
+                acc[382] += (double)v27_18_0;
+                const VT v27_19_0 = QCz * v27_9_0 + WQz * v27_9_1 + (VT)1.0 * oo2ze * v13_9_1 + (VT)2.0 * oo2e * (v27_3_0 - rho_e * v27_3_1);
+                acc[383] += (double)v27_19_0;
+                acc[384] += (double)v28_4_0;
+                acc[385] += (double)v28_5_0;
+                acc[386] += (double)v28_6_0;
+                acc[387] += (double)v28_7_0;
+                acc[388] += (double)v28_8_0;
+                acc[389] += (double)v28_9_0;
+                const VT v28_10_0 = QCx * v28_4_0 + WQx * v28_4_1 + (VT)1.0 * oo2ze * v18_4_1 + (VT)2.0 * oo2e * (v28_1_0 - rho_e * v28_1_1);
+                acc[390] += (double)v28_10_0;
+                const VT v28_11_0 = QCx * v28_5_0 + WQx * v28_5_1 + (VT)1.0 * oo2ze * v18_5_1 + (VT)1.0 * oo2e * (v28_2_0 - rho_e * v28_2_1);
+                acc[391] += (double)v28_11_0;
+                const VT v28_12_0 = QCx * v28_6_0 + WQx * v28_6_1 + (VT)1.0 * oo2ze * v18_6_1 + (VT)1.0 * oo2e * (v28_3_0 - rho_e * v28_3_1);
+                acc[392] += (double)v28_12_0;
+                const VT v28_13_0 = QCy * v28_5_0 + WQy * v28_5_1 + (VT)1.0 * oo2ze * v14_5_1 + (VT)1.0 * oo2e * (v28_1_0 - rho_e * v28_1_1);
+                acc[393] += (double)v28_13_0;
+                const VT v28_14_0 = QCz * v28_6_0 + WQz * v28_6_1 + (VT)2.0 * oo2ze * v15_6_1 + (VT)1.0 * oo2e * (v28_1_0 - rho_e * v28_1_1);
+                acc[394] += (double)v28_14_0;
+                const VT v28_15_0 = QCx * v28_8_0 + WQx * v28_8_1 + (VT)1.0 * oo2ze * v18_8_1;
+                acc[395] += (double)v28_15_0;
+                const VT v28_16_0 = QCy * v28_7_0 + WQy * v28_7_1 + (VT)1.0 * oo2ze * v14_7_1 + (VT)2.0 * oo2e * (v28_2_0 - rho_e * v28_2_1);
+                acc[396] += (double)v28_16_0;
+                const VT v28_17_0 = QCy * v28_8_0 + WQy * v28_8_1 + (VT)1.0 * oo2ze * v14_8_1 + (VT)1.0 * oo2e * (v28_3_0 - rho_e * v28_3_1);
+                acc[397] += (double)v28_17_0;
+                const VT v28_18_0 = QCz * v28_8_0 + WQz * v28_8_1 + (VT)2.0 * oo2ze * v15_8_1 + (VT)1.0 * oo2e * (v28_2_0 - rho_e * v28_2_1);
+                acc[398] += (double)v28_18_0;
+                const VT v28_19_0 = QCz * v28_9_0 + WQz * v28_9_1 + (VT)2.0 * oo2ze * v15_9_1 + (VT)2.0 * oo2e * (v28_3_0 - rho_e * v28_3_1);
+                acc[399] += (double)v28_19_0;
+                acc[400] += (double)v29_4_0;
+                acc[401] += (double)v29_5_0;
+                acc[402] += (double)v29_6_0;
+                acc[403] += (double)v29_7_0;
+                acc[404] += (double)v29_8_0;
+                acc[405] += (double)v29_9_0;
+                const VT v29_10_0 = QCx * v29_4_0 + WQx * v29_4_1 + (VT)1.0 * oo2ze * v19_4_1 + (VT)2.0 * oo2e * (v29_1_0 - rho_e * v29_1_1);
+                acc[406] += (double)v29_10_0;
+                const VT v29_11_0 = QCx * v29_5_0 + WQx * v29_5_1 + (VT)1.0 * oo2ze * v19_5_1 + (VT)1.0 * oo2e * (v29_2_0 - rho_e * v29_2_1);
+                acc[407] += (double)v29_11_0;
+                const VT v29_12_0 = QCx * v29_6_0 + WQx * v29_6_1 + (VT)1.0 * oo2ze * v19_6_1 + (VT)1.0 * oo2e * (v29_3_0 - rho_e * v29_3_1);
+                acc[408] += (double)v29_12_0;
+                const VT v29_13_0 = QCy * v29_5_0 + WQy * v29_5_1 + (VT)1.0 * oo2e * (v29_1_0 - rho_e * v29_1_1);
+                acc[409] += (double)v29_13_0;
+                const VT v29_14_0 = QCz * v29_6_0 + WQz * v29_6_1 + (VT)3.0 * oo2ze * v14_6_1 + (VT)1.0 * oo2e * (v29_1_0 - rho_e * v29_1_1);
+                acc[410] += (double)v29_14_0;
+                const VT v29_15_0 = QCx * v29_8_0 + WQx * v29_8_1 + (VT)1.0 * oo2ze * v19_8_1;
+                acc[411] += (double)v29_15_0;
+                const VT v29_16_0 = QCy * v29_7_0 + WQy * v29_7_1 + (VT)2.0 * oo2e * (v29_2_0 - rho_e * v29_2_1);
+                acc[412] += (double)v29_16_0;
+                const VT v29_17_0 = QCy * v29_8_0 + WQy * v29_8_1 + (VT)1.0 * oo2e * (v29_3_0 - rho_e * v29_3_1);
+                acc[413] += (double)v29_17_0;
+                const VT v29_18_0 = QCz * v29_8_0 + WQz * v29_8_1 + (VT)3.0 * oo2ze * v14_8_1 + (VT)1.0 * oo2e * (v29_2_0 - rho_e * v29_2_1);
+                acc[414] += (double)v29_18_0;
+                const VT v29_19_0 = QCz * v29_9_0 + WQz * v29_9_1 + (VT)3.0 * oo2ze * v14_9_1 + (VT)2.0 * oo2e * (v29_3_0 - rho_e * v29_3_1);
+                acc[415] += (double)v29_19_0;
+                acc[416] += (double)v30_4_0;
+                acc[417] += (double)v30_5_0;
+                acc[418] += (double)v30_6_0;
+                acc[419] += (double)v30_7_0;
+                acc[420] += (double)v30_8_0;
+                acc[421] += (double)v30_9_0;
+                const VT v30_10_0 = QCx * v30_4_0 + WQx * v30_4_1 + (VT)2.0 * oo2e * (v30_1_0 - rho_e * v30_1_1);
+                acc[422] += (double)v30_10_0;
+                const VT v30_11_0 = QCx * v30_5_0 + WQx * v30_5_1 + (VT)1.0 * oo2e * (v30_2_0 - rho_e * v30_2_1);
+                acc[423] += (double)v30_11_0;
+                const VT v30_12_0 = QCx * v30_6_0 + WQx * v30_6_1 + (VT)1.0 * oo2e * (v30_3_0 - rho_e * v30_3_1);
+                acc[424] += (double)v30_12_0;
+                const VT v30_13_0 = QCy * v30_5_0 + WQy * v30_5_1 + (VT)4.0 * oo2ze * v16_5_1 + (VT)1.0 * oo2e * (v30_1_0 - rho_e * v30_1_1);
+                acc[425] += (double)v30_13_0;
+                const VT v30_14_0 = QCz * v30_6_0 + WQz * v30_6_1 + (VT)1.0 * oo2e * (v30_1_0 - rho_e * v30_1_1);
+                acc[426] += (double)v30_14_0;
+                const VT v30_15_0 = QCx * v30_8_0 + WQx * v30_8_1;
+                acc[427] += (double)v30_15_0;
+                const VT v30_16_0 = QCy * v30_7_0 + WQy * v30_7_1 + (VT)4.0 * oo2ze * v16_7_1 + (VT)2.0 * oo2e * (v30_2_0 - rho_e * v30_2_1);
+                acc[428] += (double)v30_16_0;
+                const VT v30_17_0 = QCy * v30_8_0 + WQy * v30_8_1 + (VT)4.0 * oo2ze * v16_8_1 + (VT)1.0 * oo2e * (v30_3_0 - rho_e * v30_3_1);
+                acc[429] += (double)v30_17_0;
+                const VT v30_18_0 = QCz * v30_8_0 + WQz * v30_8_1 + (VT)1.0 * oo2e * (v30_2_0 - rho_e * v30_2_1);
+                acc[430] += (double)v30_18_0;
+                const VT v30_19_0 = QCz * v30_9_0 + WQz * v30_9_1 + (VT)2.0 * oo2e * (v30_3_0 - rho_e * v30_3_1);
+                acc[431] += (double)v30_19_0;
+                acc[432] += (double)v31_4_0;
+                acc[433] += (double)v31_5_0;
+                acc[434] += (double)v31_6_0;
+                acc[435] += (double)v31_7_0;
+                acc[436] += (double)v31_8_0;
+                acc[437] += (double)v31_9_0;
+                const VT v31_10_0 = QCx * v31_4_0 + WQx * v31_4_1 + (VT)2.0 * oo2e * (v31_1_0 - rho_e * v31_1_1);
+                acc[438] += (double)v31_10_0;
+                const VT v31_11_0 = QCx * v31_5_0 + WQx * v31_5_1 + (VT)1.0 * oo2e * (v31_2_0 - rho_e * v31_2_1);
+                acc[439] += (double)v31_11_0;
+                const VT v31_12_0 = QCx * v31_6_0 + WQx * v31_6_1 + (VT)1.0 * oo2e * (v31_3_0 - rho_e * v31_3_1);
+                acc[440] += (double)v31_12_0;
+                const VT v31_13_0 = QCy * v31_5_0 + WQy * v31_5_1 + (VT)3.0 * oo2ze * v17_5_1 + (VT)1.0 * oo2e * (v31_1_0 - rho_e * v31_1_1);
+                acc[441] += (double)v31_13_0;
+                const VT v31_14_0 = QCz * v31_6_0 + WQz * v31_6_1 + (VT)1.0 * oo2ze * v16_6_1 + (VT)1.0 * oo2e * (v31_1_0 - rho_e * v31_1_1);
+                acc[442] += (double)v31_14_0;
+                const VT v31_15_0 = QCx * v31_8_0 + WQx * v31_8_1;
+                acc[443] += (double)v31_15_0;
+                const VT v31_16_0 = QCy * v31_7_0 + WQy * v31_7_1 + (VT)3.0 * oo2ze * v17_7_1 + (VT)2.0 * oo2e * (v31_2_0 - rho_e * v31_2_1);
+                acc[444] += (double)v31_16_0;
+                const VT v31_17_0 = QCy * v31_8_0 + WQy * v31_8_1 + (VT)3.0 * oo2ze * v17_8_1 + (VT)1.0 * oo2e * (v31_3_0 - rho_e * v31_3_1);
+                acc[445] += (double)v31_17_0;
+                const VT v31_18_0 = QCz * v31_8_0 + WQz * v31_8_1 + (VT)1.0 * oo2ze * v16_8_1 + (VT)1.0 * oo2e * (v31_2_0 - rho_e * v31_2_1);
+                acc[446] += (double)v31_18_0;
+                const VT v31_19_0 = QCz * v31_9_0 + WQz * v31_9_1 + (VT)1.0 * oo2ze * v16_9_1 + (VT)2.0 * oo2e * (v31_3_0 - rho_e * v31_3_1);
+                acc[447] += (double)v31_19_0;
+                acc[448] += (double)v32_4_0;
+                acc[449] += (double)v32_5_0;
+                acc[450] += (double)v32_6_0;
+                acc[451] += (double)v32_7_0;
+                acc[452] += (double)v32_8_0;
+                acc[453] += (double)v32_9_0;
+                const VT v32_10_0 = QCx * v32_4_0 + WQx * v32_4_1 + (VT)2.0 * oo2e * (v32_1_0 - rho_e * v32_1_1);
+                acc[454] += (double)v32_10_0;
+                const VT v32_11_0 = QCx * v32_5_0 + WQx * v32_5_1 + (VT)1.0 * oo2e * (v32_2_0 - rho_e * v32_2_1);
+                acc[455] += (double)v32_11_0;
+                const VT v32_12_0 = QCx * v32_6_0 + WQx * v32_6_1 + (VT)1.0 * oo2e * (v32_3_0 - rho_e * v32_3_1);
+                acc[456] += (double)v32_12_0;
+                const VT v32_13_0 = QCy * v32_5_0 + WQy * v32_5_1 + (VT)2.0 * oo2ze * v18_5_1 + (VT)1.0 * oo2e * (v32_1_0 - rho_e * v32_1_1);
+                acc[457] += (double)v32_13_0;
+                const VT v32_14_0 = QCz * v32_6_0 + WQz * v32_6_1 + (VT)2.0 * oo2ze * v17_6_1 + (VT)1.0 * oo2e * (v32_1_0 - rho_e * v32_1_1);
+                acc[458] += (double)v32_14_0;
+                const VT v32_15_0 = QCx * v32_8_0 + WQx * v32_8_1;
+                acc[459] += (double)v32_15_0;
+                const VT v32_16_0 = QCy * v32_7_0 + WQy * v32_7_1 + (VT)2.0 * oo2ze * v18_7_1 + (VT)2.0 * oo2e * (v32_2_0 - rho_e * v32_2_1);
+                acc[460] += (double)v32_16_0;
+                const VT v32_17_0 = QCy * v32_8_0 + WQy * v32_8_1 + (VT)2.0 * oo2ze * v18_8_1 + (VT)1.0 * oo2e * (v32_3_0 - rho_e * v32_3_1);
+                acc[461] += (double)v32_17_0;
+                const VT v32_18_0 = QCz * v32_8_0 + WQz * v32_8_1 + (VT)2.0 * oo2ze * v17_8_1 + (VT)1.0 * oo2e * (v32_2_0 - rho_e * v32_2_1);
+                acc[462] += (double)v32_18_0;
+                const VT v32_19_0 = QCz * v32_9_0 + WQz * v32_9_1 + (VT)2.0 * oo2ze * v17_9_1 + (VT)2.0 * oo2e * (v32_3_0 - rho_e * v32_3_1);
+                acc[463] += (double)v32_19_0;
+                acc[464] += (double)v33_4_0;
+                acc[465] += (double)v33_5_0;
+                acc[466] += (double)v33_6_0;
+                acc[467] += (double)v33_7_0;
+                acc[468] += (double)v33_8_0;
+                acc[469] += (double)v33_9_0;
+                const VT v33_10_0 = QCx * v33_4_0 + WQx * v33_4_1 + (VT)2.0 * oo2e * (v33_1_0 - rho_e * v33_1_1);
+                acc[470] += (double)v33_10_0;
+                const VT v33_11_0 = QCx * v33_5_0 + WQx * v33_5_1 + (VT)1.0 * oo2e * (v33_2_0 - rho_e * v33_2_1);
+                acc[471] += (double)v33_11_0;
+                const VT v33_12_0 = QCx * v33_6_0 + WQx * v33_6_1 + (VT)1.0 * oo2e * (v33_3_0 - rho_e * v33_3_1);
+                acc[472] += (double)v33_12_0;
+                const VT v33_13_0 = QCy * v33_5_0 + WQy * v33_5_1 + (VT)1.0 * oo2ze * v19_5_1 + (VT)1.0 * oo2e * (v33_1_0 - rho_e * v33_1_1);
+                acc[473] += (double)v33_13_0;
+                const VT v33_14_0 = QCz * v33_6_0 + WQz * v33_6_1 + (VT)3.0 * oo2ze * v18_6_1 + (VT)1.0 * oo2e * (v33_1_0 - rho_e * v33_1_1);
+                acc[474] += (double)v33_14_0;
+                const VT v33_15_0 = QCx * v33_8_0 + WQx * v33_8_1;
+                acc[475] += (double)v33_15_0;
+                const VT v33_16_0 = QCy * v33_7_0 + WQy * v33_7_1 + (VT)1.0 * oo2ze * v19_7_1 + (VT)2.0 * oo2e * (v33_2_0 - rho_e * v33_2_1);
+                acc[476] += (double)v33_16_0;
+                const VT v33_17_0 = QCy * v33_8_0 + WQy * v33_8_1 + (VT)1.0 * oo2ze * v19_8_1 + (VT)1.0 * oo2e * (v33_3_0 - rho_e * v33_3_1);
+                acc[477] += (double)v33_17_0;
+                const VT v33_18_0 = QCz * v33_8_0 + WQz * v33_8_1 + (VT)3.0 * oo2ze * v18_8_1 + (VT)1.0 * oo2e * (v33_2_0 - rho_e * v33_2_1);
+                acc[478] += (double)v33_18_0;
+                const VT v33_19_0 = QCz * v33_9_0 + WQz * v33_9_1 + (VT)3.0 * oo2ze * v18_9_1 + (VT)2.0 * oo2e * (v33_3_0 - rho_e * v33_3_1);
+                acc[479] += (double)v33_19_0;
+                acc[480] += (double)v34_4_0;
+                acc[481] += (double)v34_5_0;
+                acc[482] += (double)v34_6_0;
+                acc[483] += (double)v34_7_0;
+                acc[484] += (double)v34_8_0;
+                acc[485] += (double)v34_9_0;
+                const VT v34_10_0 = QCx * v34_4_0 + WQx * v34_4_1 + (VT)2.0 * oo2e * (v34_1_0 - rho_e * v34_1_1);
+                acc[486] += (double)v34_10_0;
+                const VT v34_11_0 = QCx * v34_5_0 + WQx * v34_5_1 + (VT)1.0 * oo2e * (v34_2_0 - rho_e * v34_2_1);
+                acc[487] += (double)v34_11_0;
+                const VT v34_12_0 = QCx * v34_6_0 + WQx * v34_6_1 + (VT)1.0 * oo2e * (v34_3_0 - rho_e * v34_3_1);
+                acc[488] += (double)v34_12_0;
+                const VT v34_13_0 = QCy * v34_5_0 + WQy * v34_5_1 + (VT)1.0 * oo2e * (v34_1_0 - rho_e * v34_1_1);
+                acc[489] += (double)v34_13_0;
+                const VT v34_14_0 = QCz * v34_6_0 + WQz * v34_6_1 + (VT)4.0 * oo2ze * v19_6_1 + (VT)1.0 * oo2e * (v34_1_0 - rho_e * v34_1_1);
+                acc[490] += (double)v34_14_0;
+                const VT v34_15_0 = QCx * v34_8_0 + WQx * v34_8_1;
+                acc[491] += (double)v34_15_0;
+                const VT v34_16_0 = QCy * v34_7_0 + WQy * v34_7_1 + (VT)2.0 * oo2e * (v34_2_0 - rho_e * v34_2_1);
+                acc[492] += (double)v34_16_0;
+                const VT v34_17_0 = QCy * v34_8_0 + WQy * v34_8_1 + (VT)1.0 * oo2e * (v34_3_0 - rho_e * v34_3_1);
+                acc[493] += (double)v34_17_0;
+                const VT v34_18_0 = QCz * v34_8_0 + WQz * v34_8_1 + (VT)4.0 * oo2ze * v19_8_1 + (VT)1.0 * oo2e * (v34_2_0 - rho_e * v34_2_1);
+                acc[494] += (double)v34_18_0;
+                const VT v34_19_0 = QCz * v34_9_0 + WQz * v34_9_1 + (VT)4.0 * oo2ze * v19_9_1 + (VT)2.0 * oo2e * (v34_3_0 - rho_e * v34_3_1);
+                acc[495] += (double)v34_19_0;
+            }
         }
     }
 }

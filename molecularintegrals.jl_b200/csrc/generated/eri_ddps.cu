@@ -25,13 +25,13 @@ __device__ __forceinline__ void vrr_ddps(const PairTab &P, const BoysTab &B, int
             const double r = rsqrt(bra.zeta + ket.zeta);
             const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
-            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[6];
             boys_fm<5>(T, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
-            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
             const VT WQx = (VT)(zz * PQx), WQy = (VT)(zz * PQy), WQz = (VT)(zz * PQz);
             const VT oo2z = (VT)bra.oo2z, oo2e = (VT)ket.oo2z, oo2ze = (VT)(0.5 * r2);
@@ -144,192 +144,288 @@ __device__ __forceinline__ void vrr_ddps(const PairTab &P, const BoysTab &B, int
             const VT v33_0_1 = PAz * v18_0_1 + WPz * v18_0_2 + (VT)2.0 * oo2z * (v8_0_1 - rho_z * v8_0_2);
             const VT v34_0_0 = PAz * v19_0_0 + WPz * v19_0_1 + (VT)3.0 * oo2z * (v9_0_0 - rho_z * v9_0_1);
             const VT v34_0_1 = PAz * v19_0_1 + WPz * v19_0_2 + (VT)3.0 * oo2z * (v9_0_1 - rho_z * v9_0_2);
-            const VT v4_1_0 = QCx * v4_0_0 + WQx * v4_0_1 + (VT)2.0 * oo2ze * v1_0_1;
-            const VT v5_1_0 = QCx * v5_0_0 + WQx * v5_0_1 + (VT)1.0 * oo2ze * v2_0_1;
-            const VT v6_1_0 = QCx * v6_0_0 + WQx * v6_0_1 + (VT)1.0 * oo2ze * v3_0_1;
-            const VT v7_1_0 = QCx * v7_0_0 + WQx * v7_0_1;
-            const VT v8_1_0 = QCx * v8_0_0 + WQx * v8_0_1;
-            const VT v9_1_0 = QCx * v9_0_0 + WQx * v9_0_1;
-            const VT v10_1_0 = QCx * v10_0_0 + WQx * v10_0_1 + (VT)3.0 * oo2ze * v4_0_1;
-            const VT v11_1_0 = QCx * v11_0_0 + WQx * v11_0_1 + (VT)2.0 * oo2ze * v5_0_1;
-            const VT v12_1_0 = QCx * v12_0_0 + WQx * v12_0_1 + (VT)2.0 * oo2ze * v6_0_1;
-            const VT v13_1_0 = QCx * v13_0_0 + WQx * v13_0_1 + (VT)1.0 * oo2ze * v7_0_1;
-            const VT v14_1_0 = QCx * v14_0_0 + WQx * v14_0_1 + (VT)1.0 * oo2ze * v9_0_1;
-            const VT v15_1_0 = QCx * v15_0_0 + WQx * v15_0_1 + (VT)1.0 * oo2ze * v8_0_1;
-            const VT v16_1_0 = QCx * v16_0_0 + WQx * v16_0_1;
-            const VT v17_1_0 = QCx * v17_0_0 + WQx * v17_0_1;
-            const VT v18_1_0 = QCx * v18_0_0 + WQx * v18_0_1;
-            const VT v19_1_0 = QCx * v19_0_0 + WQx * v19_0_1;
-            const VT v20_1_0 = QCx * v20_0_0 + WQx * v20_0_1 + (VT)4.0 * oo2ze * v10_0_1;
-            const VT v21_1_0 = QCx * v21_0_0 + WQx * v21_0_1 + (VT)3.0 * oo2ze * v11_0_1;
-            const VT v22_1_0 = QCx * v22_0_0 + WQx * v22_0_1 + (VT)3.0 * oo2ze * v12_0_1;
-            const VT v23_1_0 = QCx * v23_0_0 + WQx * v23_0_1 + (VT)2.0 * oo2ze * v13_0_1;
-            const VT v24_1_0 = QCx * v24_0_0 + WQx * v24_0_1 + (VT)2.0 * oo2ze * v15_0_1;
-            const VT v25_1_0 = QCx * v25_0_0 + WQx * v25_0_1 + (VT)2.0 * oo2ze * v14_0_1;
-            const VT v26_1_0 = QCx * v26_0_0 + WQx * v26_0_1 + (VT)1.0 * oo2ze * v16_0_1;
-            const VT v27_1_0 = QCx * v27_0_0 + WQx * v27_0_1 + (VT)1.0 * oo2ze * v17_0_1;
-            const VT v28_1_0 = QCx * v28_0_0 + WQx * v28_0_1 + (VT)1.0 * oo2ze * v18_0_1;
-            const VT v29_1_0 = QCx * v29_0_0 + WQx * v29_0_1 + (VT)1.0 * oo2ze * v19_0_1;
-            const VT v30_1_0 = QCx * v30_0_0 + WQx * v30_0_1;
-            const VT v31_1_0 = QCx * v31_0_0 + WQx * v31_0_1;
-            const VT v32_1_0 = QCx * v32_0_0 + WQx * v32_0_1;
-            const VT v33_1_0 = QCx * v33_0_0 + WQx * v33_0_1;
-            const VT v34_1_0 = QCx * v34_0_0 + WQx * v34_0_1;
-            const VT v4_2_0 = QCy * v4_0_0 + WQy * v4_0_1;
-            const VT v5_2_0 = QCy * v5_0_0 + WQy * v5_0_1 + (VT)1.0 * oo2ze * v1_0_1;
-            const VT v6_2_0 = QCy * v6_0_0 + WQy * v6_0_1;
-            const VT v7_2_0 = QCy * v7_0_0 + WQy * v7_0_1 + (VT)2.0 * oo2ze * v2_0_1;
-            const VT v8_2_0 = QCy * v8_0_0 + WQy * v8_0_1 + (VT)1.0 * oo2ze * v3_0_1;
-            const VT v9_2_0 = QCy * v9_0_0 + WQy * v9_0_1;
-            const VT v10_2_0 = QCy * v10_0_0 + WQy * v10_0_1;
-            const VT v11_2_0 = QCy * v11_0_0 + WQy * v11_0_1 + (VT)1.0 * oo2ze * v4_0_1;
-            const VT v12_2_0 = QCy * v12_0_0 + WQy * v12_0_1;
-            const VT v13_2_0 = QCy * v13_0_0 + WQy * v13_0_1 + (VT)2.0 * oo2ze * v5_0_1;
-            const VT v14_2_0 = QCy * v14_0_0 + WQy * v14_0_1;
-            const VT v15_2_0 = QCy * v15_0_0 + WQy * v15_0_1 + (VT)1.0 * oo2ze * v6_0_1;
-            const VT v16_2_0 = QCy * v16_0_0 + WQy * v16_0_1 + (VT)3.0 * oo2ze * v7_0_1;
-            const VT v17_2_0 = QCy * v17_0_0 + WQy * v17_0_1 + (VT)2.0 * oo2ze * v8_0_1;
-            const VT v18_2_0 = QCy * v18_0_0 + WQy * v18_0_1 + (VT)1.0 * oo2ze * v9_0_1;
-            const VT v19_2_0 = QCy * v19_0_0 + WQy * v19_0_1;
-            const VT v20_2_0 = QCy * v20_0_0 + WQy * v20_0_1;
-            const VT v21_2_0 = QCy * v21_0_0 + WQy * v21_0_1 + (VT)1.0 * oo2ze * v10_0_1;
-            const VT v22_2_0 = QCy * v22_0_0 + WQy * v22_0_1;
-            const VT v23_2_0 = QCy * v23_0_0 + WQy * v23_0_1 + (VT)2.0 * oo2ze * v11_0_1;
-            const VT v24_2_0 = QCy * v24_0_0 + WQy * v24_0_1 + (VT)1.0 * oo2ze * v12_0_1;
-            const VT v25_2_0 = QCy * v25_0_0 + WQy * v25_0_1;
-            const VT v26_2_0 = QCy * v26_0_0 + WQy * v26_0_1 + (VT)3.0 * oo2ze * v13_0_1;
-            const VT v27_2_0 = QCy * v27_0_0 + WQy * v27_0_1 + (VT)2.0 * oo2ze * v15_0_1;
-            const VT v28_2_0 = QCy * v28_0_0 + WQy * v28_0_1 + (VT)1.0 * oo2ze * v14_0_1;
-            const VT v29_2_0 = QCy * v29_0_0 + WQy * v29_0_1;
-            const VT v30_2_0 = QCy * v30_0_0 + WQy * v30_0_1 + (VT)4.0 * oo2ze * v16_0_1;
-            const VT v31_2_0 = QCy * v31_0_0 + WQy * v31_0_1 + (VT)3.0 * oo2ze * v17_0_1;
-            const VT v32_2_0 = QCy * v32_0_0 + WQy * v32_0_1 + (VT)2.0 * oo2ze * v18_0_1;
-            const VT v33_2_0 = QCy * v33_0_0 + WQy * v33_0_1 + (VT)1.0 * oo2ze * v19_0_1;
-            const VT v34_2_0 = QCy * v34_0_0 + WQy * v34_0_1;
-            const VT v4_3_0 = QCz * v4_0_0 + WQz * v4_0_1;
-            const VT v5_3_0 = QCz * v5_0_0 + WQz * v5_0_1;
-            const VT v6_3_0 = QCz * v6_0_0 + WQz * v6_0_1 + (VT)1.0 * oo2ze * v1_0_1;
-            const VT v7_3_0 = QCz * v7_0_0 + WQz * v7_0_1;
-            const VT v8_3_0 = QCz * v8_0_0 + WQz * v8_0_1 + (VT)1.0 * oo2ze * v2_0_1;
-            const VT v9_3_0 = QCz * v9_0_0 + WQz * v9_0_1 + (VT)2.0 * oo2ze * v3_0_1;
-            const VT v10_3_0 = QCz * v10_0_0 + WQz * v10_0_1;
-            const VT v11_3_0 = QCz * v11_0_0 + WQz * v11_0_1;
-            const VT v12_3_0 = QCz * v12_0_0 + WQz * v12_0_1 + (VT)1.0 * oo2ze * v4_0_1;
-            const VT v13_3_0 = QCz * v13_0_0 + WQz * v13_0_1;
-            const VT v14_3_0 = QCz * v14_0_0 + WQz * v14_0_1 + (VT)2.0 * oo2ze * v6_0_1;
-            const VT v15_3_0 = QCz * v15_0_0 + WQz * v15_0_1 + (VT)1.0 * oo2ze * v5_0_1;
-            const VT v16_3_0 = QCz * v16_0_0 + WQz * v16_0_1;
-            const VT v17_3_0 = QCz * v17_0_0 + WQz * v17_0_1 + (VT)1.0 * oo2ze * v7_0_1;
-            const VT v18_3_0 = QCz * v18_0_0 + WQz * v18_0_1 + (VT)2.0 * oo2ze * v8_0_1;
-            const VT v19_3_0 = QCz * v19_0_0 + WQz * v19_0_1 + (VT)3.0 * oo2ze * v9_0_1;
-            const VT v20_3_0 = QCz * v20_0_0 + WQz * v20_0_1;
-            const VT v21_3_0 = QCz * v21_0_0 + WQz * v21_0_1;
-            const VT v22_3_0 = QCz * v22_0_0 + WQz * v22_0_1 + (VT)1.0 * oo2ze * v10_0_1;
-            const VT v23_3_0 = QCz * v23_0_0 + WQz * v23_0_1;
-            const VT v24_3_0 = QCz * v24_0_0 + WQz * v24_0_1 + (VT)1.0 * oo2ze * v11_0_1;
-            const VT v25_3_0 = QCz * v25_0_0 + WQz * v25_0_1 + (VT)2.0 * oo2ze * v12_0_1;
-            const VT v26_3_0 = QCz * v26_0_0 + WQz * v26_0_1;
-            const VT v27_3_0 = QCz * v27_0_0 + WQz * v27_0_1 + (VT)1.0 * oo2ze * v13_0_1;
-            const VT v28_3_0 = QCz * v28_0_0 + WQz * v28_0_1 + (VT)2.0 * oo2ze * v15_0_1;
-            const VT v29_3_0 = QCz * v29_0_0 + WQz * v29_0_1 + (VT)3.0 * oo2ze * v14_0_1;
-            const VT v30_3_0 = QCz * v30_0_0 + WQz * v30_0_1;
-            const VT v31_3_0 = QCz * v31_0_0 + WQz * v31_0_1 + (VT)1.0 * oo2ze * v16_0_1;
-            const VT v32_3_0 = QCz * v32_0_0 + WQz * v32_0_1 + (VT)2.0 * oo2ze * v17_0_1;
-            const VT v33_3_0 = QCz * v33_0_0 + WQz * v33_0_1 + (VT)3.0 * oo2ze * v18_0_1;
-            const VT v34_3_0 = QCz * v34_0_0 + WQz * v34_0_1 + (VT)4.0 * oo2ze * v19_0_1;
-            acc[0] += (double)v4_1_0;
-            acc[1] += (double)v4_2_0;
-            acc[2] += (double)v4_3_0;
-            acc[3] += (double)v5_1_0;
-            acc[4] += (double)v5_2_0;
-            acc[5] += (double)v5_3_0;
-            acc[6] += (double)v6_1_0;
-            acc[7] += (double)v6_2_0;
-            acc[8] += (double)v6_3_0;
-            acc[9] += (double)v7_1_0;
-            acc[10] += (double)v7_2_0;
-            acc[11] += (double)v7_3_0;
-            acc[12] += (double)v8_1_0;
-            acc[13] += (double)v8_2_0;
-            acc[14] += (double)v8_3_0;
-            acc[15] += (double)v9_1_0;
-            acc[16] += (double)v9_2_0;
-            acc[17] += (double)v9_3_0;
-            acc[18] += (double)v10_1_0;
-            acc[19] += (double)v10_2_0;
-            acc[20] += (double)v10_3_0;
-            acc[21] += (double)v11_1_0;
-            acc[22] += (double)v11_2_0;
-            acc[23] += (double)v11_3_0;
-            acc[24] += (double)v12_1_0;
-            acc[25] += (double)v12_2_0;
-            acc[26] += (double)v12_3_0;
-            acc[27] += (double)v13_1_0;
-            acc[28] += (double)v13_2_0;
-            acc[29] += (double)v13_3_0;
-            acc[30] += (double)v14_1_0;
-            acc[31] += (double)v14_2_0;
-            acc[32] += (double)v14_3_0;
-            acc[33] += (double)v15_1_0;
-            acc[34] += (double)v15_2_0;
-            acc[35] += (double)v15_3_0;
-            acc[36] += (double)v16_1_0;
-            acc[37] += (double)v16_2_0;
-            acc[38] += (double)v16_3_0;
-            acc[39] += (double)v17_1_0;
-            acc[40] += (double)v17_2_0;
-            acc[41] += (double)v17_3_0;
-            acc[42] += (double)v18_1_0;
-            acc[43] += (double)v18_2_0;
-            acc[44] += (double)v18_3_0;
-            acc[45] += (double)v19_1_0;
-            acc[46] += (double)v19_2_0;
-            acc[47] += (double)v19_3_0;
-            acc[48] += (double)v20_1_0;
-            acc[49] += (double)v20_2_0;
-            acc[50] += (double)v20_3_0;
-            acc[51] += (double)v21_1_0;
-            acc[52] += (double)v21_2_0;
-            acc[53] += (double)v21_3_0;
-            acc[54] += (double)v22_1_0;
-            acc[55] += (double)v22_2_0;
-            acc[56] += (double)v22_3_0;
-            acc[57] += (double)v23_1_0;
-            acc[58] += (double)v23_2_0;
-            acc[59] += (double)v23_3_0;
-            acc[60] += (double)v24_1_0;
-            acc[61] += (double)v24_2_0;
-            acc[62] += (double)v24_3_0;
-            acc[63] += (double)v25_1_0;
-            acc[64] += (double)v25_2_0;
-            acc[65] += (double)v25_3_0;
-            acc[66] += (double)v26_1_0;
-            acc[67] += (double)v26_2_0;
-            acc[68] += (double)v26_3_0;
-            acc[69] += (double)v27_1_0;
-            acc[70] += (double)v27_2_0;
-            acc[71] += (double)v27_3_0;
-            acc[72] += (double)v28_1_0;
-            acc[73] += (double)v28_2_0;
-            acc[74] += (double)v28_3_0;
-            acc[75] += (double)v29_1_0;
-            acc[76] += (double)v29_2_0;
-            acc[77] += (double)v29_3_0;
-            acc[78] += (double)v30_1_0;
-            acc[79] += (double)v30_2_0;
-            acc[80] += (double)v30_3_0;
-            acc[81] += (double)v31_1_0;
-            acc[82] += (double)v31_2_0;
-            acc[83] += (double)v31_3_0;
-            acc[84] += (double)v32_1_0;
-            acc[85] += (double)v32_2_0;
-            acc[86] += (double)v32_3_0;
-            acc[87] += (double)v33_1_0;
-            acc[88] += (double)v33_2_0;
-            acc[89] += (double)v33_3_0;
-            acc[90] += (double)v34_1_0;
-            acc[91] += (double)v34_2_0;
-            acc[92] += (double)v34_3_0;
+            if constexpr (sizeof(VT) == 8) {
+                acc[0] = fma(QCx, v4_0_0, fma(WQx, v4_0_1, fma(2.0 * oo2ze, v1_0_1, acc[0])));
+                acc[1] = fma(QCy, v4_0_0, fma(WQy, v4_0_1, acc[1]));
+                acc[2] = fma(QCz, v4_0_0, fma(WQz, v4_0_1, acc[2]));
+                acc[3] = fma(QCx, v5_0_0, fma(WQx, v5_0_1, fma(1.0 * oo2ze, v2_0_1, acc[3])));
+                acc[4] = fma(QCy, v5_0_0, fma(WQy, v5_0_1, fma(1.0 * oo2ze, v1_0_1, acc[4])));
+                acc[5] = fma(QCz, v5_0_0, fma(WQz, v5_0_1, acc[5]));
+                acc[6] = fma(QCx, v6_0_0, fma(WQx, v6_0_1, fma(1.0 * oo2ze, v3_0_1, acc[6])));
+                acc[7] = fma(QCy, v6_0_0, fma(WQy, v6_0_1, acc[7]));
+                acc[8] = fma(QCz, v6_0_0, fma(WQz, v6_0_1, fma(1.0 * oo2ze, v1_0_1, acc[8])));
+                acc[9] = fma(QCx, v7_0_0, fma(WQx, v7_0_1, acc[9]));
+                acc[10] = fma(QCy, v7_0_0, fma(WQy, v7_0_1, fma(2.0 * oo2ze, v2_0_1, acc[10])));
+                acc[11] = fma(QCz, v7_0_0, fma(WQz, v7_0_1, acc[11]));
+                acc[12] = fma(QCx, v8_0_0, fma(WQx, v8_0_1, acc[12]));
+                acc[13] = fma(QCy, v8_0_0, fma(WQy, v8_0_1, fma(1.0 * oo2ze, v3_0_1, acc[13])));
+                acc[14] = fma(QCz, v8_0_0, fma(WQz, v8_0_1, fma(1.0 * oo2ze, v2_0_1, acc[14])));
+                acc[15] = fma(QCx, v9_0_0, fma(WQx, v9_0_1, acc[15]));
+                acc[16] = fma(QCy, v9_0_0, fma(WQy, v9_0_1, acc[16]));
+                acc[17] = fma(QCz, v9_0_0, fma(WQz, v9_0_1, fma(2.0 * oo2ze, v3_0_1, acc[17])));
+                acc[18] = fma(QCx, v10_0_0, fma(WQx, v10_0_1, fma(3.0 * oo2ze, v4_0_1, acc[18])));
+                acc[19] = fma(QCy, v10_0_0, fma(WQy, v10_0_1, acc[19]));
+                acc[20] = fma(QCz, v10_0_0, fma(WQz, v10_0_1, acc[20]));
+                acc[21] = fma(QCx, v11_0_0, fma(WQx, v11_0_1, fma(2.0 * oo2ze, v5_0_1, acc[21])));
+                acc[22] = fma(QCy, v11_0_0, fma(WQy, v11_0_1, fma(1.0 * oo2ze, v4_0_1, acc[22])));
+                acc[23] = fma(QCz, v11_0_0, fma(WQz, v11_0_1, acc[23]));
+                acc[24] = fma(QCx, v12_0_0, fma(WQx, v12_0_1, fma(2.0 * oo2ze, v6_0_1, acc[24])));
+                acc[25] = fma(QCy, v12_0_0, fma(WQy, v12_0_1, acc[25]));
+                acc[26] = fma(QCz, v12_0_0, fma(WQz, v12_0_1, fma(1.0 * oo2ze, v4_0_1, acc[26])));
+                acc[27] = fma(QCx, v13_0_0, fma(WQx, v13_0_1, fma(1.0 * oo2ze, v7_0_1, acc[27])));
+                acc[28] = fma(QCy, v13_0_0, fma(WQy, v13_0_1, fma(2.0 * oo2ze, v5_0_1, acc[28])));
+                acc[29] = fma(QCz, v13_0_0, fma(WQz, v13_0_1, acc[29]));
+                acc[30] = fma(QCx, v14_0_0, fma(WQx, v14_0_1, fma(1.0 * oo2ze, v9_0_1, acc[30])));
+                acc[31] = fma(QCy, v14_0_0, fma(WQy, v14_0_1, acc[31]));
+                acc[32] = fma(QCz, v14_0_0, fma(WQz, v14_0_1, fma(2.0 * oo2ze, v6_0_1, acc[32])));
+                acc[33] = fma(QCx, v15_0_0, fma(WQx, v15_0_1, fma(1.0 * oo2ze, v8_0_1, acc[33])));
+                acc[34] = fma(QCy, v15_0_0, fma(WQy, v15_0_1, fma(1.0 * oo2ze, v6_0_1, acc[34])));
+                acc[35] = fma(QCz, v15_0_0, fma(WQz, v15_0_1, fma(1.0 * oo2ze, v5_0_1, acc[35])));
+                acc[36] = fma(QCx, v16_0_0, fma(WQx, v16_0_1, acc[36]));
+                acc[37] = fma(QCy, v16_0_0, fma(WQy, v16_0_1, fma(3.0 * oo2ze, v7_0_1, acc[37])));
+                acc[38] = fma(QCz, v16_0_0, fma(WQz, v16_0_1, acc[38]));
+                acc[39] = fma(QCx, v17_0_0, fma(WQx, v17_0_1, acc[39]));
+                acc[40] = fma(QCy, v17_0_0, fma(WQy, v17_0_1, fma(2.0 * oo2ze, v8_0_1, acc[40])));
+                acc[41] = fma(QCz, v17_0_0, fma(WQz, v17_0_1, fma(1.0 * oo2ze, v7_0_1, acc[41])));
+                acc[42] = fma(QCx, v18_0_0, fma(WQx, v18_0_1, acc[42]));
+                acc[43] = fma(QCy, v18_0_0, fma(WQy, v18_0_1, fma(1.0 * oo2ze, v9_0_1, acc[43])));
+                acc[44] = fma(QCz, v18_0_0, fma(WQz, v18_0_1, fma(2.0 * oo2ze, v8_0_1, acc[44])));
+                acc[45] = fma(QCx, v19_0_0, fma(WQx, v19_0_1, acc[45]));
+                acc[46] = fma(QCy, v19_0_0, fma(WQy, v19_0_1, acc[46]));
+                acc[47] = fma(QCz, v19_0_0, fma(WQz, v19_0_1, fma(3.0 * oo2ze, v9_0_1, acc[47])));
+                acc[48] = fma(QCx, v20_0_0, fma(WQx, v20_0_1, fma(4.0 * oo2ze, v10_0_1, acc[48])));
+                acc[49] = fma(QCy, v20_0_0, fma(WQy, v20_0_1, acc[49]));
+                acc[50] = fma(QCz, v20_0_0, fma(WQz, v20_0_1, acc[50]));
+                acc[51] = fma(QCx, v21_0_0, fma(WQx, v21_0_1, fma(3.0 * oo2ze, v11_0_1, acc[51])));
+                acc[52] = fma(QCy, v21_0_0, fma(WQy, v21_0_1, fma(1.0 * oo2ze, v10_0_1, acc[52])));
+                acc[53] = fma(QCz, v21_0_0, fma(WQz, v21_0_1, acc[53]));
+                acc[54] = fma(QCx, v22_0_0, fma(WQx, v22_0_1, fma(3.0 * oo2ze, v12_0_1, acc[54])));
+                acc[55] = fma(QCy, v22_0_0, fma(WQy, v22_0_1, acc[55]));
+                acc[56] = fma(QCz, v22_0_0, fma(WQz, v22_0_1, fma(1.0 * oo2ze, v10_0_1, acc[56])));
+                acc[57] = fma(QCx, v23_0_0, fma(WQx, v23_0_1, fma(2.0 * oo2ze, v13_0_1, acc[57])));
+                acc[58] = fma(QCy, v23_0_0, fma(WQy, v23_0_1, fma(2.0 * oo2ze, v11_0_1, acc[58])));
+                acc[59] = fma(QCz, v23_0_0, fma(WQz, v23_0_1, acc[59]));
+                acc[60] = fma(QCx, v24_0_0, fma(WQx, v24_0_1, fma(2.0 * oo2ze, v15_0_1, acc[60])));
+                acc[61] = fma(QCy, v24_0_0, fma(WQy, v24_0_1, fma(1.0 * oo2ze, v12_0_1, acc[61])));
+                acc[62] = fma(QCz, v24_0_0, fma(WQz, v24_0_1, fma(1.0 * oo2ze, v11_0_1, acc[62])));
+                acc[63] = fma(QCx, v25_0_0, fma(WQx, v25_0_1, fma(2.0 * oo2ze, v14_0_1, acc[63])));
+                acc[64] = fma(QCy, v25_0_0, fma(WQy, v25_0_1, acc[64]));
+                acc[65] = fma(QCz, v25_0_0, fma(WQz, v25_0_1, fma(2.0 * oo2ze, v12_0_1, acc[65])));
+                acc[66] = fma(QCx, v26_0_0, fma(WQx, v26_0_1, fma(1.0 * oo2ze, v16_0_1, acc[66])));
+                acc[67] = fma(QCy, v26_0_0, fma(WQy, v26_0_1, fma(3.0 * oo2ze, v13_0_1, acc[67])));
+                acc[68] = fma(QCz, v26_0_0, fma(WQz, v26_0_1, acc[68]));
+                acc[69] = fma(QCx, v27_0_0, fma(WQx, v27_0_1, fma(1.0 * oo2ze, v17_0_1, acc[69])));
+                acc[70] = fma(QCy, v27_0_0, fma(WQy, v27_0_1, fma(2.0 * oo2ze, v15_0_1, acc[70])));
+                acc[71] = fma(QCz, v27_0_0, fma(WQz, v27_0_1, fma(1.0 * oo2ze, v13_0_1, acc[71])));
+                acc[72] = fma(QCx, v28_0_0, fma(WQx, v28_0_1, fma(1.0 * oo2ze, v18_0_1, acc[72])));
+                acc[73] = fma(QCy, v28_0_0, fma(WQy, v28_0_1, fma(1.0 * oo2ze, v14_0_1, acc[73])));
+                acc[74] = fma(QCz, v28_0_0, fma(WQz, v28_0_1, fma(2.0 * oo2ze, v15_0_1, acc[74])));
+                acc[75] = fma(QCx, v29_0_0, fma(WQx, v29_0_1, fma(1.0 * oo2ze, v19_0_1, acc[75])));
+                acc[76] = fma(QCy, v29_0_0, fma(WQy, v29_0_1, acc[76]));
+                acc[77] = fma(QCz, v29_0_0, fma(WQz, v29_0_1, fma(3.0 * oo2ze, v14_0_1, acc[77])));
+                acc[78] = fma(QCx, v30_0_0, fma(WQx, v30_0_1, acc[78]));
+                acc[79] = fma(QCy, v30_0_0, fma(WQy, v30_0_1, fma(4.0 * oo2ze, v16_0_1, acc[79])));
+                acc[80] = fma(QCz, v30_0_0, fma(WQz, v30_0_1, acc[80]));
+                acc[81] = fma(QCx, v31_0_0, fma(WQx, v31_0_1, acc[81]));
+                acc[82] = fma(QCy, v31_0_0, fma(WQy, v31_0_1, fma(3.0 * oo2ze, v17_0_1, acc[82])));
+                acc[83] = fma(QCz, v31_0_0, fma(WQz, v31_0_1, fma(1.0 * oo2ze, v16_0_1, acc[83])));
+                acc[84] = fma(QCx, v32_0_0, fma(WQx, v32_0_1, acc[84]));
+                acc[85] = fma(QCy, v32_0_0, fma(WQy, v32_0_1, fma(2.0 * oo2ze, v18_0_1, acc[85])));
+                acc[86] = fma(QCz, v32_0_0, fma(WQz, v32_0_1, fma(2.0 * oo2ze, v17_0_1, acc[86])));
+                acc[87] = fma(QCx, v33_0_0, fma(WQx, v33_0_1, acc[87]));
+                acc[88] = fma(QCy, v33_0_0, fma(WQy, v33_0_1, fma(1.0 * oo2ze, v19_0_1, acc[88])));
+                acc[89] = fma(QCz, v33_0_0, fma(WQz, v33_0_1, fma(3.0 * oo2ze, v18_0_1, acc[89])));
+                acc[90] = fma(QCx, v34_0_0, fma(WQx, v34_0_1, acc[90]));
+                acc[91] = fma(QCy, v34_0_0, fma(WQy, v34_0_1, acc[91]));
+                acc[92] = fma(QCz, v34_0_0, fma(WQz, v34_0_1, fma(4.0 * oo2ze, v19_0_1, acc[92])));
+            } else {
+                const VT v4_1_0 = QCx * v4_0_0 + WQx * v4_0_1 + (VT)2.0 * oo2ze * v1_0_1;
+                acc[0] += (double)v4_1_0;
+                const VT v4_2_0 = QCy * v4_0_0 + WQy * v4_0_1;
+                acc[1] += (double)v4_2_0;
+                const VT v4_3_0 = QCz * v4_0_0 + WQz * v4_0_1;
+                acc[2] += (double)v4_3_0;
+                const VT v5_1_0 = QCx * v5_0_0 + WQx * v5_0_1 + (VT)1.0 * oo2ze * v2_0_1;
+                acc[3] += (double)v5_1_0;
+                const VT v5_2_0 = QCy * v5_0_0 + WQy * v5_0_1 + (VT)1.0 * oo2ze * v1_0_1;
+                acc[4] += (double)v5_2_0;
+                const VT v5_3_0 = QCz * v5_0_0 + WQz * v5_0_1;
+                acc[5] += (double)v5_3_0;
+                const VT v6_1_0 = QCx * v6_0_0 + WQx * v6_0_1 + (VT)1.0 * oo2ze * v3_0_1;
+                acc[6] += (double)v6_1_0;
+                const VT v6_2_0 = QCy * v6_0_0 + WQy * v6_0_1;
+                acc[7] += (double)v6_2_0;
+                const VT v6_3_0 = QCz * v6_0_0 + WQz * v6_0_1 + (VT)1.0 * oo2ze * v1_0_1;
+                acc[8] += (double)v6_3_0;
+                const VT v7_1_0 = QCx * v7_0_0 + WQx * v7_0_1;
+                acc[9] += (double)v7_1_0;
+                const VT v7_2_0 = QCy * v7_0_0 + WQy * v7_0_1 + (VT)2.0 * oo2ze * v2_0_1;
+                acc[10] += (double)v7_2_0;
+                const VT v7_3_0 = QCz * v7_0_0 + WQz * v7_0_1;
+                acc[11] += (double)v7_3_0;
+                const VT v8_1_0 = QCx * v8_0_0 + WQx * v8_0_1;
+                acc[12] += (double)v8_1_0;
+                const VT v8_2_0 = QCy * v8_0_0 + WQy * v8_0_1 + (VT)1.0 * oo2ze * v3_0_1;
+                acc[13] += (double)v8_2_0;
+                const VT v8_3_0 = QCz * v8_0_0 + WQz * v8_0_1 + (VT)1.0 * oo2ze * v2_0_1;
+                acc[14] += (double)v8_3_0;
+                const VT v9_1_0 = QCx * v9_0_0 + WQx * v9_0_1;
+                acc[15] += (double)v9_1_0;
+                const VT v9_2_0 = QCy * v9_0_0 + WQy * v9_0_1;
+                acc[16] += (double)v9_2_0;
+                const VT v9_3_0 = QCz * v9_0_0 + WQz * v9_0_1 + (VT)2.0 * oo2ze * v3_0_1;
+                acc[17] += (double)v9_3_0;
+                const VT v10_1_0 = QCx * v10_0_0 + WQx * v10_0_1 + (VT)3.0 * oo2ze * v4_0_1;
+                acc[18] += (double)v10_1_0;
+                const VT v10_2_0 = QCy * v10_0_0 + WQy * v10_0_1;
+                acc[19] += (double)v10_2_0;
+                const VT v10_3_0 = QCz * v10_0_0 + WQz * v10_0_1;
+                acc[20] += (double)v10_3_0;
+                const VT v11_1_0 = QCx * v11_0_0 + WQx * v11_0_1 + (VT)2.0 * oo2ze * v5_0_1;
+                acc[21] += (double)v11_1_0;
+                const VT v11_2_0 = QCy * v11_0_0 + WQy * v11_0_1 + (VT)1.0 * oo2ze * v4_0_1;
+                acc[22] += (double)v11_2_0;
+                const VT v11_3_0 = QCz * v11_0_0 + WQz * v11_0_1;
+                acc[23] += (double)v11_3_0;
+                const VT v12_1_0 = QCx * v12_0_0 + WQx * v12_0_1 + (VT)2.0 * oo2ze * v6_0_1;
+                acc[24] += (double)v12_1_0;
+                const VT v12_2_0 = QCy * v12_0_0 + WQy * v12_0_1;
+                acc[25] += (double)v12_2_0;
+                const VT v12_3_0 = QCz * v12_0_0 + WQz * v12_0_1 + (VT)1.0 * oo2ze * v4_0_1;
+                acc[26] += (double)v12_3_0;
+                const VT v13_1_0 = QCx * v13_0_0 + WQx * v13_0_1 + (VT)1.0 * oo2ze * v7_0_1;
+                acc[27] += (double)v13_1_0;
+                const VT v13_2_0 = QCy * v13_0_0 + WQy * v13_0_1 + (VT)2.0 * oo2ze * v5_0_1;
+                acc[28] += (double)v13_2_0;
+                const VT v13_3_0 = QCz * v13_0_0 + WQz * v13_0_1;
+                acc[29] += (double)v13_3_0;
+                const VT v14_1_0 = QCx * v14_0_0 + WQx * v14_0_1 + (VT)1.0 * oo2ze * v9_0_1;
+                acc[30] += (double)v14_1_0;
+                const VT v14_2_0 = QCy * v14_0_0 + WQy * v14_0_1;
+                acc[31] += (double)v14_2_0;
+                const VT v14_3_0 = QCz * v14_0_0 + WQz * v14_0_1 + (VT)2.0 * oo2ze * v6_0_1;
+                acc[32] += (double)v14_3_0;
+                const VT v15_1_0 = QCx * v15_0_0 + WQx * v15_0_1 + (VT)1.0 * oo2ze * v8_0_1;
+                acc[33] += (double)v15_1_0;
+                const VT v15_2_0 = QCy * v15_0_0 + WQy * v15_0_1 + (VT)1.0 * oo2ze * v6_0_1;
+                acc[34] += (double)v15_2_0;
+                const VT v15_3_0 = QCz * v15_0_0 + WQz * v15_0_1 + (VT)1.0 * oo2ze * v5_0_1;
+                acc[35] += (double)v15_3_0;
+                const VT v16_1_0 = QCx * v16_0_0 + WQx * v16_0_1;
+                acc[36] += (double)v16_1_0;
+                const VT v16_2_0 = QCy * v16_0_0 + WQy * v16_0_1 + (VT)3.0 * oo2ze * v7_0_1;
+                acc[37] += (double)v16_2_0;
+                const VT v16_3_0 = QCz * v16_0_0 + WQz * v16_0_1;
+                acc[38] += (double)v16_3_0;
+                const VT v17_1_0 = QCx * v17_0_0 + WQx * v17_0_1;
+                acc[39] += (double)v17_1_0;
+                const VT v17_2_0 = QCy * v17_0_0 + WQy * v17_0_1 + (VT)2.0 * oo2ze * v8_0_1;
+                acc[40] += (double)v17_2_0;
+                const VT v17_3_0 = QCz * v17_0_0 + WQz * v17_0_1 + (VT)1.0 * oo2ze * v7_0_1;
+                acc[41] += (double)v17_3_0;
+                const VT v18_1_0 = QCx * v18_0_0 + WQx * v18_0_1;
+                acc[42] += (double)v18_1_0;
+                const VT v18_2_0 = QCy * v18_0_0 + WQy * v18_0_1 + (VT)1.0 * oo2ze * v9_0_1;
+                acc[43] += (double)v18_2_0;
+                const VT v18_3_0 = QCz * v18_0_0 + WQz * v18_0_1 + (VT)2.0 * oo2ze * v8_0_1;
+                acc[44] += (double)v18_3_0;
+                const VT v19_1_0 = QCx * v19_0_0 + WQx * v19_0_1;
+                acc[45] += (double)v19_1_0;
+                const VT v19_2_0 = QCy * v19_0_0 + WQy * v19_0_1;
+                acc[46] += (double)v19_2_0;
+                const VT v19_3_0 = QCz * v19_0_0 + WQz * v19_0_1 + (VT)3.0 * oo2ze * v9_0_1;
+                acc[47] += (double)v19_3_0;
+                const VT v20_1_0 = QCx * v20_0_0 + WQx * v20_0_1 + (VT)4.0 * oo2ze * v10_0_1;
+                acc[48] += (double)v20_1_0;
+                const VT v20_2_0 = QCy * v20_0_0 + WQy * v20_0_1;
+                acc[49] += (double)v20_2_0;
+                const VT v20_3_0 = QCz * v20_0_0 + WQz * v20_0_1;
+                acc[50] += (double)v20_3_0;
+                const VT v21_1_0 = QCx * v21_0_0 + WQx * v21_0_1 + (VT)3.0 * oo2ze * v11_0_1;
+                acc[51] += (double)v21_1_0;
+                const VT v21_2_0 = QCy * v21_0_0 + WQy * v21_0_1 + (VT)1.0 * oo2ze * v10_0_1;
+                acc[52] += (double)v21_2_0;
+                const VT v21_3_0 = QCz * v21_0_0 + WQz * v21_0_1;
+                acc[53] += (double)v21_3_0;
+                const VT v22_1_0 = QCx * v22_0_0 + WQx * v22_0_1 + (VT)3.0 * oo2ze * v12_0_1;
+                acc[54] += (double)v22_1_0;
+                const VT v22_2_0 = QCy * v22_0_0 + WQy * v22_0_1;
+                acc[55] += (double)v22_2_0;
+                const VT v22_3_0 = QCz * v22_0_0 + WQz * v22_0_1 + (VT)1.0 * oo2ze * v10_0_1;
+                acc[56] += (double)v22_3_0;
+                const VT v23_1_0 = QCx * v23_0_0 + WQx * v23_0_1 + (VT)2.0 * oo2ze * v13_0_1;
+                acc[57] += (double)v23_1_0;
+                const VT v23_2_0 = QCy * v23_0_0 + WQy * v23_0_1 + (VT)2.0 * oo2ze * v11_0_1;
+                acc[58] += (double)v23_2_0;
+                const VT v23_3_0 = QCz * v23_0_0 + WQz * v23_0_1;
+                acc[59] += (double)v23_3_0;
+                const VT v24_1_0 = QCx * v24_0_0 + WQx * v24_0_1 + (VT)2.0 * oo2ze * v15_0_1;
+                acc[60] += (double)v24_1_0;
+                const VT v24_2_0 = QCy * v24_0_0 + WQy * v24_0_1 + (VT)1.0 * oo2ze * v12_0_1;
+                acc[61] += (double)v24_2_0;
+                const VT v24_3_0 = QCz * v24_0_0 + WQz * v24_0_1 + (VT)1.0 * oo2ze * v11_0_1;
+                acc[62] += (double)v24_3_0;
+                const VT v25_1_0 = QCx * v25_0_0 + WQx * v25_0_1 + (VT)2.0 * oo2ze * v14_0_1;
+                acc[63] += (double)v25_1_0;
+                const VT v25_2_0 = QCy * v25_0_0 + WQy * v25_0_1;
+                acc[64] += (double)v25_2_0;
+                const VT v25_3_0 = QCz * v25_0_0 + WQz * v25_0_1 + (VT)2.0 * oo2ze * v12_0_1;
+                acc[65] += (double)v25_3_0;
+                const VT v26_1_0 = QCx * v26_0_0 + WQx * v26_0_1 + (VT)1.0 * oo2ze * v16_0_1;
+                acc[66] += (double)v26_1_0;
+                const VT v26_2_0 = QCy * v26_0_0 + WQy * v26_0_1 + (VT)3.0 * oo2ze * v13_0_1;
+                acc[67] += (double)v26_2_0;
+                const VT v26_3_0 = QCz * v26_0_0 + WQz * v26_0_1;
+                acc[68] += (double)v26_3_0;
+                const VT v27_1_0 = QCx * v27_0_0 + WQx * v27_0_1 + (VT)1.0 * oo2ze * v17_0_1;
+                acc[69] += (double)v27_1_0;
+                const VT v27_2_0 = QCy * v27_0_0 + WQy * v27_0_1 + (VT)2.0 * oo2ze * v15_0_1;
+                acc[70] += (double)v27_2_0;
+                const VT v27_3_0 = QCz * v27_0_0 + WQz * v27_0_1 + (VT)1.0 * oo2ze * v13_0_1;
+                acc[71] += (double)v27_3_0;
+                const VT v28_1_0 = QCx * v28_0_0 + WQx * v28_0_1 + (VT)1.0 * oo2ze * v18_0_1;
+                acc[72] += (double)v28_1_0;
+                const VT v28_2_0 = QCy * v28_0_0 + WQy * v28_0_1 + (VT)1.0 * oo2ze * v14_0_1;
+                acc[73] += (double)v28_2_0;
+                const VT v28_3_0 = QCz * v28_0_0 + WQz * v28_0_1 + (VT)2.0 * oo2ze * v15_0_1;
+                acc[74] += (double)v28_3_0;
+                const VT v29_1_0 = QCx * v29_0_0 + WQx * v29_0_1 + (VT)1.0 * oo2ze * v19_0_1;
+                acc[75] += (double)v29_1_0;
+                const VT v29_2_0 = QCy * v29_0_0 + WQy * v29_0_1;
+                acc[76] += (double)v29_2_0;
+                const VT v29_3_0 = QCz * v29_0_0 + WQz * v29_0_1 + (VT)3.0 * oo2ze * v14_0_1;
+                acc[77] += (double)v29_3_0;
+                const VT v30_1_0 = QCx * v30_0_0 + WQx * v30_0_1;
+                acc[78] += (double)v30_1_0;
+                const VT v30_2_0 = QCy * v30_0_0 + WQy * v30_0_1 + (VT)4.0 * oo2ze * v16_0_1;
+                acc[79] += (double)v30_2_0;
+                const VT v30_3_0 = QCz * v30_0_0 + WQz * v30_0_1;
+                acc[80] += (double)v30_3_0;
+                const VT v31_1_0 = QCx * v31_0_0 + WQx * v31_0_1;
+                acc[81] += (double)v31_1_0;
+                const VT v31_2_0 = QCy * v31_0_0 + WQy * v31_0_1 + (VT)3.0 * oo2ze * v17_0_1;
+                acc[82] += (double)v31_2_0;
+                const VT v31_3_0 = QCz * v31_0_0 + WQz * v31_0_1 + (VT)1.0 * oo2ze * v16_0_1;
+                acc[83] += (double)v31_3_0;
+                const VT v32_1_0 = QCx * v32_0_0 + WQx * v32_0_1;
+                acc[84] += (double)v32_1_0;
+                const VT v32_2_0 = QCy * v32_0_0 + WQy * v32_0_1 + (VT)2.0 * oo2ze * v18_0_1;
+                acc[85] += (double)v32_2_0;
+                const VT v32_3_0 = QCz * v32_0_0 + WQz * v32_0_1 + (VT)2.0 * oo2ze * v17_0_1;
+                acc[86] += (double)v32_3_0;
+                const VT v33_1_0 = QCx * v33_0_0 + WQx * v33_0_1;
+                acc[87] += (double)v33_1_0;
+                const VT v33_2_0 = QCy * v33_0_0 + WQy * v33_0_1 + (VT)1.0 * oo2ze * v19_0_1;
+                acc[88] += (double)v33_2_0;
+                const VT v33_3_0 = QCz * v33_0_0 + WQz * v33_0_1 + (VT)3.0 * oo2ze * v18_0_1;
+                acc[89] += (double)v33_3_0;
+                const VT v34_1_0 = QCx * v34_0_0 + WQx * v34_0_1;
+                acc[90] += (double)v34_1_0;
+                const VT v34_2_0 = QCy * v34_0_0 + WQy * v34_0_1;
+                acc[91] += (double)v34_2_0;
+                const VT v34_3_0 = QCz * v34_0_0 + WQz * v34_0_1 + (VT)4.0 * oo2ze * v19_0_1;
+                acc[92] += (double)v34_3_0;
+            }
         }
     }
 }

@@ -25,13 +25,13 @@ __device__ __forceinline__ void vrr_dpdp(const PairTab &P, const BoysTab &B, int
             const double r = rsqrt(bra.zeta + ket.zeta);
             const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
-            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[7];
             boys_fm<6>(T, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
-            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
             const VT WQx = (VT)(zz * PQx), WQy = (VT)(zz * PQy), WQz = (VT)(zz * PQz);
             const VT oo2z = (VT)bra.oo2z, oo2e = (VT)ket.oo2z, oo2ze = (VT)(0.5 * r2);
@@ -509,422 +509,681 @@ __device__ __forceinline__ void vrr_dpdp(const PairTab &P, const BoysTab &B, int
             const VT v18_9_1 = QCz * v18_3_1 + WQz * v18_3_2 + (VT)2.0 * oo2ze * v8_3_2 + (VT)1.0 * oo2e * (v18_0_1 - rho_e * v18_0_2);
             const VT v19_9_0 = QCz * v19_3_0 + WQz * v19_3_1 + (VT)3.0 * oo2ze * v9_3_1 + (VT)1.0 * oo2e * (v19_0_0 - rho_e * v19_0_1);
             const VT v19_9_1 = QCz * v19_3_1 + WQz * v19_3_2 + (VT)3.0 * oo2ze * v9_3_2 + (VT)1.0 * oo2e * (v19_0_1 - rho_e * v19_0_2);
-            const VT v4_10_0 = QCx * v4_4_0 + WQx * v4_4_1 + (VT)2.0 * oo2ze * v1_4_1 + (VT)2.0 * oo2e * (v4_1_0 - rho_e * v4_1_1);
-            const VT v5_10_0 = QCx * v5_4_0 + WQx * v5_4_1 + (VT)1.0 * oo2ze * v2_4_1 + (VT)2.0 * oo2e * (v5_1_0 - rho_e * v5_1_1);
-            const VT v6_10_0 = QCx * v6_4_0 + WQx * v6_4_1 + (VT)1.0 * oo2ze * v3_4_1 + (VT)2.0 * oo2e * (v6_1_0 - rho_e * v6_1_1);
-            const VT v7_10_0 = QCx * v7_4_0 + WQx * v7_4_1 + (VT)2.0 * oo2e * (v7_1_0 - rho_e * v7_1_1);
-            const VT v8_10_0 = QCx * v8_4_0 + WQx * v8_4_1 + (VT)2.0 * oo2e * (v8_1_0 - rho_e * v8_1_1);
-            const VT v9_10_0 = QCx * v9_4_0 + WQx * v9_4_1 + (VT)2.0 * oo2e * (v9_1_0 - rho_e * v9_1_1);
-            const VT v10_10_0 = QCx * v10_4_0 + WQx * v10_4_1 + (VT)3.0 * oo2ze * v4_4_1 + (VT)2.0 * oo2e * (v10_1_0 - rho_e * v10_1_1);
-            const VT v11_10_0 = QCx * v11_4_0 + WQx * v11_4_1 + (VT)2.0 * oo2ze * v5_4_1 + (VT)2.0 * oo2e * (v11_1_0 - rho_e * v11_1_1);
-            const VT v12_10_0 = QCx * v12_4_0 + WQx * v12_4_1 + (VT)2.0 * oo2ze * v6_4_1 + (VT)2.0 * oo2e * (v12_1_0 - rho_e * v12_1_1);
-            const VT v13_10_0 = QCx * v13_4_0 + WQx * v13_4_1 + (VT)1.0 * oo2ze * v7_4_1 + (VT)2.0 * oo2e * (v13_1_0 - rho_e * v13_1_1);
-            const VT v14_10_0 = QCx * v14_4_0 + WQx * v14_4_1 + (VT)1.0 * oo2ze * v9_4_1 + (VT)2.0 * oo2e * (v14_1_0 - rho_e * v14_1_1);
-            const VT v15_10_0 = QCx * v15_4_0 + WQx * v15_4_1 + (VT)1.0 * oo2ze * v8_4_1 + (VT)2.0 * oo2e * (v15_1_0 - rho_e * v15_1_1);
-            const VT v16_10_0 = QCx * v16_4_0 + WQx * v16_4_1 + (VT)2.0 * oo2e * (v16_1_0 - rho_e * v16_1_1);
-            const VT v17_10_0 = QCx * v17_4_0 + WQx * v17_4_1 + (VT)2.0 * oo2e * (v17_1_0 - rho_e * v17_1_1);
-            const VT v18_10_0 = QCx * v18_4_0 + WQx * v18_4_1 + (VT)2.0 * oo2e * (v18_1_0 - rho_e * v18_1_1);
-            const VT v19_10_0 = QCx * v19_4_0 + WQx * v19_4_1 + (VT)2.0 * oo2e * (v19_1_0 - rho_e * v19_1_1);
-            const VT v4_11_0 = QCx * v4_5_0 + WQx * v4_5_1 + (VT)2.0 * oo2ze * v1_5_1 + (VT)1.0 * oo2e * (v4_2_0 - rho_e * v4_2_1);
-            const VT v5_11_0 = QCx * v5_5_0 + WQx * v5_5_1 + (VT)1.0 * oo2ze * v2_5_1 + (VT)1.0 * oo2e * (v5_2_0 - rho_e * v5_2_1);
-            const VT v6_11_0 = QCx * v6_5_0 + WQx * v6_5_1 + (VT)1.0 * oo2ze * v3_5_1 + (VT)1.0 * oo2e * (v6_2_0 - rho_e * v6_2_1);
-            const VT v7_11_0 = QCx * v7_5_0 + WQx * v7_5_1 + (VT)1.0 * oo2e * (v7_2_0 - rho_e * v7_2_1);
-            const VT v8_11_0 = QCx * v8_5_0 + WQx * v8_5_1 + (VT)1.0 * oo2e * (v8_2_0 - rho_e * v8_2_1);
-            const VT v9_11_0 = QCx * v9_5_0 + WQx * v9_5_1 + (VT)1.0 * oo2e * (v9_2_0 - rho_e * v9_2_1);
-            const VT v10_11_0 = QCx * v10_5_0 + WQx * v10_5_1 + (VT)3.0 * oo2ze * v4_5_1 + (VT)1.0 * oo2e * (v10_2_0 - rho_e * v10_2_1);
-            const VT v11_11_0 = QCx * v11_5_0 + WQx * v11_5_1 + (VT)2.0 * oo2ze * v5_5_1 + (VT)1.0 * oo2e * (v11_2_0 - rho_e * v11_2_1);
-            const VT v12_11_0 = QCx * v12_5_0 + WQx * v12_5_1 + (VT)2.0 * oo2ze * v6_5_1 + (VT)1.0 * oo2e * (v12_2_0 - rho_e * v12_2_1);
-            const VT v13_11_0 = QCx * v13_5_0 + WQx * v13_5_1 + (VT)1.0 * oo2ze * v7_5_1 + (VT)1.0 * oo2e * (v13_2_0 - rho_e * v13_2_1);
-            const VT v14_11_0 = QCx * v14_5_0 + WQx * v14_5_1 + (VT)1.0 * oo2ze * v9_5_1 + (VT)1.0 * oo2e * (v14_2_0 - rho_e * v14_2_1);
-            const VT v15_11_0 = QCx * v15_5_0 + WQx * v15_5_1 + (VT)1.0 * oo2ze * v8_5_1 + (VT)1.0 * oo2e * (v15_2_0 - rho_e * v15_2_1);
-            const VT v16_11_0 = QCx * v16_5_0 + WQx * v16_5_1 + (VT)1.0 * oo2e * (v16_2_0 - rho_e * v16_2_1);
-            const VT v17_11_0 = QCx * v17_5_0 + WQx * v17_5_1 + (VT)1.0 * oo2e * (v17_2_0 - rho_e * v17_2_1);
-            const VT v18_11_0 = QCx * v18_5_0 + WQx * v18_5_1 + (VT)1.0 * oo2e * (v18_2_0 - rho_e * v18_2_1);
-            const VT v19_11_0 = QCx * v19_5_0 + WQx * v19_5_1 + (VT)1.0 * oo2e * (v19_2_0 - rho_e * v19_2_1);
-            const VT v4_12_0 = QCx * v4_6_0 + WQx * v4_6_1 + (VT)2.0 * oo2ze * v1_6_1 + (VT)1.0 * oo2e * (v4_3_0 - rho_e * v4_3_1);
-            const VT v5_12_0 = QCx * v5_6_0 + WQx * v5_6_1 + (VT)1.0 * oo2ze * v2_6_1 + (VT)1.0 * oo2e * (v5_3_0 - rho_e * v5_3_1);
-            const VT v6_12_0 = QCx * v6_6_0 + WQx * v6_6_1 + (VT)1.0 * oo2ze * v3_6_1 + (VT)1.0 * oo2e * (v6_3_0 - rho_e * v6_3_1);
-            const VT v7_12_0 = QCx * v7_6_0 + WQx * v7_6_1 + (VT)1.0 * oo2e * (v7_3_0 - rho_e * v7_3_1);
-            const VT v8_12_0 = QCx * v8_6_0 + WQx * v8_6_1 + (VT)1.0 * oo2e * (v8_3_0 - rho_e * v8_3_1);
-            const VT v9_12_0 = QCx * v9_6_0 + WQx * v9_6_1 + (VT)1.0 * oo2e * (v9_3_0 - rho_e * v9_3_1);
-            const VT v10_12_0 = QCx * v10_6_0 + WQx * v10_6_1 + (VT)3.0 * oo2ze * v4_6_1 + (VT)1.0 * oo2e * (v10_3_0 - rho_e * v10_3_1);
-            const VT v11_12_0 = QCx * v11_6_0 + WQx * v11_6_1 + (VT)2.0 * oo2ze * v5_6_1 + (VT)1.0 * oo2e * (v11_3_0 - rho_e * v11_3_1);
-            const VT v12_12_0 = QCx * v12_6_0 + WQx * v12_6_1 + (VT)2.0 * oo2ze * v6_6_1 + (VT)1.0 * oo2e * (v12_3_0 - rho_e * v12_3_1);
-            const VT v13_12_0 = QCx * v13_6_0 + WQx * v13_6_1 + (VT)1.0 * oo2ze * v7_6_1 + (VT)1.0 * oo2e * (v13_3_0 - rho_e * v13_3_1);
-            const VT v14_12_0 = QCx * v14_6_0 + WQx * v14_6_1 + (VT)1.0 * oo2ze * v9_6_1 + (VT)1.0 * oo2e * (v14_3_0 - rho_e * v14_3_1);
-            const VT v15_12_0 = QCx * v15_6_0 + WQx * v15_6_1 + (VT)1.0 * oo2ze * v8_6_1 + (VT)1.0 * oo2e * (v15_3_0 - rho_e * v15_3_1);
-            const VT v16_12_0 = QCx * v16_6_0 + WQx * v16_6_1 + (VT)1.0 * oo2e * (v16_3_0 - rho_e * v16_3_1);
-            const VT v17_12_0 = QCx * v17_6_0 + WQx * v17_6_1 + (VT)1.0 * oo2e * (v17_3_0 - rho_e * v17_3_1);
-            const VT v18_12_0 = QCx * v18_6_0 + WQx * v18_6_1 + (VT)1.0 * oo2e * (v18_3_0 - rho_e * v18_3_1);
-            const VT v19_12_0 = QCx * v19_6_0 + WQx * v19_6_1 + (VT)1.0 * oo2e * (v19_3_0 - rho_e * v19_3_1);
-            const VT v4_13_0 = QCy * v4_5_0 + WQy * v4_5_1 + (VT)1.0 * oo2e * (v4_1_0 - rho_e * v4_1_1);
-            const VT v5_13_0 = QCy * v5_5_0 + WQy * v5_5_1 + (VT)1.0 * oo2ze * v1_5_1 + (VT)1.0 * oo2e * (v5_1_0 - rho_e * v5_1_1);
-            const VT v6_13_0 = QCy * v6_5_0 + WQy * v6_5_1 + (VT)1.0 * oo2e * (v6_1_0 - rho_e * v6_1_1);
-            const VT v7_13_0 = QCy * v7_5_0 + WQy * v7_5_1 + (VT)2.0 * oo2ze * v2_5_1 + (VT)1.0 * oo2e * (v7_1_0 - rho_e * v7_1_1);
-            const VT v8_13_0 = QCy * v8_5_0 + WQy * v8_5_1 + (VT)1.0 * oo2ze * v3_5_1 + (VT)1.0 * oo2e * (v8_1_0 - rho_e * v8_1_1);
-            const VT v9_13_0 = QCy * v9_5_0 + WQy * v9_5_1 + (VT)1.0 * oo2e * (v9_1_0 - rho_e * v9_1_1);
-            const VT v10_13_0 = QCy * v10_5_0 + WQy * v10_5_1 + (VT)1.0 * oo2e * (v10_1_0 - rho_e * v10_1_1);
-            const VT v11_13_0 = QCy * v11_5_0 + WQy * v11_5_1 + (VT)1.0 * oo2ze * v4_5_1 + (VT)1.0 * oo2e * (v11_1_0 - rho_e * v11_1_1);
-            const VT v12_13_0 = QCy * v12_5_0 + WQy * v12_5_1 + (VT)1.0 * oo2e * (v12_1_0 - rho_e * v12_1_1);
-            const VT v13_13_0 = QCy * v13_5_0 + WQy * v13_5_1 + (VT)2.0 * oo2ze * v5_5_1 + (VT)1.0 * oo2e * (v13_1_0 - rho_e * v13_1_1);
-            const VT v14_13_0 = QCy * v14_5_0 + WQy * v14_5_1 + (VT)1.0 * oo2e * (v14_1_0 - rho_e * v14_1_1);
-            const VT v15_13_0 = QCy * v15_5_0 + WQy * v15_5_1 + (VT)1.0 * oo2ze * v6_5_1 + (VT)1.0 * oo2e * (v15_1_0 - rho_e * v15_1_1);
-            const VT v16_13_0 = QCy * v16_5_0 + WQy * v16_5_1 + (VT)3.0 * oo2ze * v7_5_1 + (VT)1.0 * oo2e * (v16_1_0 - rho_e * v16_1_1);
-            const VT v17_13_0 = QCy * v17_5_0 + WQy * v17_5_1 + (VT)2.0 * oo2ze * v8_5_1 + (VT)1.0 * oo2e * (v17_1_0 - rho_e * v17_1_1);
-            const VT v18_13_0 = QCy * v18_5_0 + WQy * v18_5_1 + (VT)1.0 * oo2ze * v9_5_1 + (VT)1.0 * oo2e * (v18_1_0 - rho_e * v18_1_1);
-            const VT v19_13_0 = QCy * v19_5_0 + WQy * v19_5_1 + (VT)1.0 * oo2e * (v19_1_0 - rho_e * v19_1_1);
-            const VT v4_14_0 = QCz * v4_6_0 + WQz * v4_6_1 + (VT)1.0 * oo2e * (v4_1_0 - rho_e * v4_1_1);
-            const VT v5_14_0 = QCz * v5_6_0 + WQz * v5_6_1 + (VT)1.0 * oo2e * (v5_1_0 - rho_e * v5_1_1);
-            const VT v6_14_0 = QCz * v6_6_0 + WQz * v6_6_1 + (VT)1.0 * oo2ze * v1_6_1 + (VT)1.0 * oo2e * (v6_1_0 - rho_e * v6_1_1);
-            const VT v7_14_0 = QCz * v7_6_0 + WQz * v7_6_1 + (VT)1.0 * oo2e * (v7_1_0 - rho_e * v7_1_1);
-            const VT v8_14_0 = QCz * v8_6_0 + WQz * v8_6_1 + (VT)1.0 * oo2ze * v2_6_1 + (VT)1.0 * oo2e * (v8_1_0 - rho_e * v8_1_1);
-            const VT v9_14_0 = QCz * v9_6_0 + WQz * v9_6_1 + (VT)2.0 * oo2ze * v3_6_1 + (VT)1.0 * oo2e * (v9_1_0 - rho_e * v9_1_1);
-            const VT v10_14_0 = QCz * v10_6_0 + WQz * v10_6_1 + (VT)1.0 * oo2e * (v10_1_0 - rho_e * v10_1_1);
-            const VT v11_14_0 = QCz * v11_6_0 + WQz * v11_6_1 + (VT)1.0 * oo2e * (v11_1_0 - rho_e * v11_1_1);
-            const VT v12_14_0 = QCz * v12_6_0 + WQz * v12_6_1 + (VT)1.0 * oo2ze * v4_6_1 + (VT)1.0 * oo2e * (v12_1_0 - rho_e * v12_1_1);
-            const VT v13_14_0 = QCz * v13_6_0 + WQz * v13_6_1 + (VT)1.0 * oo2e * (v13_1_0 - rho_e * v13_1_1);
-            const VT v14_14_0 = QCz * v14_6_0 + WQz * v14_6_1 + (VT)2.0 * oo2ze * v6_6_1 + (VT)1.0 * oo2e * (v14_1_0 - rho_e * v14_1_1);
-            const VT v15_14_0 = QCz * v15_6_0 + WQz * v15_6_1 + (VT)1.0 * oo2ze * v5_6_1 + (VT)1.0 * oo2e * (v15_1_0 - rho_e * v15_1_1);
-            const VT v16_14_0 = QCz * v16_6_0 + WQz * v16_6_1 + (VT)1.0 * oo2e * (v16_1_0 - rho_e * v16_1_1);
-            const VT v17_14_0 = QCz * v17_6_0 + WQz * v17_6_1 + (VT)1.0 * oo2ze * v7_6_1 + (VT)1.0 * oo2e * (v17_1_0 - rho_e * v17_1_1);
-            const VT v18_14_0 = QCz * v18_6_0 + WQz * v18_6_1 + (VT)2.0 * oo2ze * v8_6_1 + (VT)1.0 * oo2e * (v18_1_0 - rho_e * v18_1_1);
-            const VT v19_14_0 = QCz * v19_6_0 + WQz * v19_6_1 + (VT)3.0 * oo2ze * v9_6_1 + (VT)1.0 * oo2e * (v19_1_0 - rho_e * v19_1_1);
-            const VT v4_15_0 = QCx * v4_8_0 + WQx * v4_8_1 + (VT)2.0 * oo2ze * v1_8_1;
-            const VT v5_15_0 = QCx * v5_8_0 + WQx * v5_8_1 + (VT)1.0 * oo2ze * v2_8_1;
-            const VT v6_15_0 = QCx * v6_8_0 + WQx * v6_8_1 + (VT)1.0 * oo2ze * v3_8_1;
-            const VT v7_15_0 = QCx * v7_8_0 + WQx * v7_8_1;
-            const VT v8_15_0 = QCx * v8_8_0 + WQx * v8_8_1;
-            const VT v9_15_0 = QCx * v9_8_0 + WQx * v9_8_1;
-            const VT v10_15_0 = QCx * v10_8_0 + WQx * v10_8_1 + (VT)3.0 * oo2ze * v4_8_1;
-            const VT v11_15_0 = QCx * v11_8_0 + WQx * v11_8_1 + (VT)2.0 * oo2ze * v5_8_1;
-            const VT v12_15_0 = QCx * v12_8_0 + WQx * v12_8_1 + (VT)2.0 * oo2ze * v6_8_1;
-            const VT v13_15_0 = QCx * v13_8_0 + WQx * v13_8_1 + (VT)1.0 * oo2ze * v7_8_1;
-            const VT v14_15_0 = QCx * v14_8_0 + WQx * v14_8_1 + (VT)1.0 * oo2ze * v9_8_1;
-            const VT v15_15_0 = QCx * v15_8_0 + WQx * v15_8_1 + (VT)1.0 * oo2ze * v8_8_1;
-            const VT v16_15_0 = QCx * v16_8_0 + WQx * v16_8_1;
-            const VT v17_15_0 = QCx * v17_8_0 + WQx * v17_8_1;
-            const VT v18_15_0 = QCx * v18_8_0 + WQx * v18_8_1;
-            const VT v19_15_0 = QCx * v19_8_0 + WQx * v19_8_1;
-            const VT v4_16_0 = QCy * v4_7_0 + WQy * v4_7_1 + (VT)2.0 * oo2e * (v4_2_0 - rho_e * v4_2_1);
-            const VT v5_16_0 = QCy * v5_7_0 + WQy * v5_7_1 + (VT)1.0 * oo2ze * v1_7_1 + (VT)2.0 * oo2e * (v5_2_0 - rho_e * v5_2_1);
-            const VT v6_16_0 = QCy * v6_7_0 + WQy * v6_7_1 + (VT)2.0 * oo2e * (v6_2_0 - rho_e * v6_2_1);
-            const VT v7_16_0 = QCy * v7_7_0 + WQy * v7_7_1 + (VT)2.0 * oo2ze * v2_7_1 + (VT)2.0 * oo2e * (v7_2_0 - rho_e * v7_2_1);
-            const VT v8_16_0 = QCy * v8_7_0 + WQy * v8_7_1 + (VT)1.0 * oo2ze * v3_7_1 + (VT)2.0 * oo2e * (v8_2_0 - rho_e * v8_2_1);
-            const VT v9_16_0 = QCy * v9_7_0 + WQy * v9_7_1 + (VT)2.0 * oo2e * (v9_2_0 - rho_e * v9_2_1);
-            const VT v10_16_0 = QCy * v10_7_0 + WQy * v10_7_1 + (VT)2.0 * oo2e * (v10_2_0 - rho_e * v10_2_1);
-            const VT v11_16_0 = QCy * v11_7_0 + WQy * v11_7_1 + (VT)1.0 * oo2ze * v4_7_1 + (VT)2.0 * oo2e * (v11_2_0 - rho_e * v11_2_1);
-            const VT v12_16_0 = QCy * v12_7_0 + WQy * v12_7_1 + (VT)2.0 * oo2e * (v12_2_0 - rho_e * v12_2_1);
-            const VT v13_16_0 = QCy * v13_7_0 + WQy * v13_7_1 + (VT)2.0 * oo2ze * v5_7_1 + (VT)2.0 * oo2e * (v13_2_0 - rho_e * v13_2_1);
-            const VT v14_16_0 = QCy * v14_7_0 + WQy * v14_7_1 + (VT)2.0 * oo2e * (v14_2_0 - rho_e * v14_2_1);
-            const VT v15_16_0 = QCy * v15_7_0 + WQy * v15_7_1 + (VT)1.0 * oo2ze * v6_7_1 + (VT)2.0 * oo2e * (v15_2_0 - rho_e * v15_2_1);
-            const VT v16_16_0 = QCy * v16_7_0 + WQy * v16_7_1 + (VT)3.0 * oo2ze * v7_7_1 + (VT)2.0 * oo2e * (v16_2_0 - rho_e * v16_2_1);
-            const VT v17_16_0 = QCy * v17_7_0 + WQy * v17_7_1 + (VT)2.0 * oo2ze * v8_7_1 + (VT)2.0 * oo2e * (v17_2_0 - rho_e * v17_2_1);
-            const VT v18_16_0 = QCy * v18_7_0 + WQy * v18_7_1 + (VT)1.0 * oo2ze * v9_7_1 + (VT)2.0 * oo2e * (v18_2_0 - rho_e * v18_2_1);
-            const VT v19_16_0 = QCy * v19_7_0 + WQy * v19_7_1 + (VT)2.0 * oo2e * (v19_2_0 - rho_e * v19_2_1);
-            const VT v4_17_0 = QCy * v4_8_0 + WQy * v4_8_1 + (VT)1.0 * oo2e * (v4_3_0 - rho_e * v4_3_1);
-            const VT v5_17_0 = QCy * v5_8_0 + WQy * v5_8_1 + (VT)1.0 * oo2ze * v1_8_1 + (VT)1.0 * oo2e * (v5_3_0 - rho_e * v5_3_1);
-            const VT v6_17_0 = QCy * v6_8_0 + WQy * v6_8_1 + (VT)1.0 * oo2e * (v6_3_0 - rho_e * v6_3_1);
-            const VT v7_17_0 = QCy * v7_8_0 + WQy * v7_8_1 + (VT)2.0 * oo2ze * v2_8_1 + (VT)1.0 * oo2e * (v7_3_0 - rho_e * v7_3_1);
-            const VT v8_17_0 = QCy * v8_8_0 + WQy * v8_8_1 + (VT)1.0 * oo2ze * v3_8_1 + (VT)1.0 * oo2e * (v8_3_0 - rho_e * v8_3_1);
-            const VT v9_17_0 = QCy * v9_8_0 + WQy * v9_8_1 + (VT)1.0 * oo2e * (v9_3_0 - rho_e * v9_3_1);
-            const VT v10_17_0 = QCy * v10_8_0 + WQy * v10_8_1 + (VT)1.0 * oo2e * (v10_3_0 - rho_e * v10_3_1);
-            const VT v11_17_0 = QCy * v11_8_0 + WQy * v11_8_1 + (VT)1.0 * oo2ze * v4_8_1 + (VT)1.0 * oo2e * (v11_3_0 - rho_e * v11_3_1);
-            const VT v12_17_0 = QCy * v12_8_0 + WQy * v12_8_1 + (VT)1.0 * oo2e * (v12_3_0 - rho_e * v12_3_1);
-            const VT v13_17_0 = QCy * v13_8_0 + WQy * v13_8_1 + (VT)2.0 * oo2ze * v5_8_1 + (VT)1.0 * oo2e * (v13_3_0 - rho_e * v13_3_1);
-            const VT v14_17_0 = QCy * v14_8_0 + WQy * v14_8_1 + (VT)1.0 * oo2e * (v14_3_0 - rho_e * v14_3_1);
-            const VT v15_17_0 = QCy * v15_8_0 + WQy * v15_8_1 + (VT)1.0 * oo2ze * v6_8_1 + (VT)1.0 * oo2e * (v15_3_0 - rho_e * v15_3_1);
-            const VT v16_17_0 = QCy * v16_8_0 + WQy * v16_8_1 + (VT)3.0 * oo2ze * v7_8_1 + (VT)1.0 * oo2e * (v16_3_0 - rho_e * v16_3_1);
-            const VT v17_17_0 = QCy * v17_8_0 + WQy * v17_8_1 + (VT)2.0 * oo2ze * v8_8_1 + (VT)1.0 * oo2e * (v17_3_0 - rho_e * v17_3_1);
-            const VT v18_17_0 = QCy * v18_8_0 + WQy * v18_8_1 + (VT)1.0 * oo2ze * v9_8_1 + (VT)1.0 * oo2e * (v18_3_0 - rho_e * v18_3_1);
-            const VT v19_17_0 = QCy * v19_8_0 + WQy * v19_8_1 + (VT)1.0 * oo2e * (v19_3_0 - rho_e * v19_3_1);
-            const VT v4_18_0 = QCz * v4_8_0 + WQz * v4_8_1 + (VT)1.0 * oo2e * (v4_2_0 - rho_e * v4_2_1);
-            const VT v5_18_0 = QCz * v5_8_0 + WQz * v5_8_1 + (VT)1.0 * oo2e * (v5_2_0 - rho_e * v5_2_1);
-            const VT v6_18_0 = QCz * v6_8_0 + WQz * v6_8_1 + (VT)1.0 * oo2ze * v1_8_1 + (VT)1.0 * oo2e * (v6_2_0 - rho_e * v6_2_1);
-            const VT v7_18_0 = QCz * v7_8_0 + WQz * v7_8_1 + (VT)1.0 * oo2e * (v7_2_0 - rho_e * v7_2_1);
-            const VT v8_18_0 = QCz * v8_8_0 + WQz * v8_8_1 + (VT)1.0 * oo2ze * v2_8_1 + (VT)1.0 * oo2e * (v8_2_0 - rho_e * v8_2_1);
-            const VT v9_18_0 = QCz * v9_8_0 + WQz * v9_8_1 + (VT)2.0 * oo2ze * v3_8_1 + (VT)1.0 * oo2e * (v9_2_0 - rho_e * v9_2_1);
-            const VT v10_18_0 = QCz * v10_8_0 + WQz * v10_8_1 + (VT)1.0 * oo2e * (v10_2_0 - rho_e * v10_2_1);
-            const VT v11_18_0 = QCz * v11_8_0 + WQz * v11_8_1 + (VT)1.0 * oo2e * (v11_2_0 - rho_e * v11_2_1);
-            const VT v12_18_0 = QCz * v12_8_0 + WQz * v12_8_1 + (VT)1.0 * oo2ze * v4_8_1 + (VT)1.0 * oo2e * (v12_2_0 - rho_e * v12_2_1);
-            const VT v13_18_0 = QCz * v13_8_0 + WQz * v13_8_1 + (VT)1.0 * oo2e * (v13_2_0 - rho_e * v13_2_1);
-            const VT v14_18_0 = QCz * v14_8_0 + WQz * v14_8_1 + (VT)2.0 * oo2ze * v6_8_1 + (VT)1.0 * oo2e * (v14_2_0 - rho_e * v14_2_1);
-            const VT v15_18_0 = QCz * v15_8_0 + WQz * v15_8_1 + (VT)1.0 * oo2ze * v5_8_1 + (VT)1.0 * oo2e * (v15_2_0 - rho_e * v15_2_1);
-            const VT v16_18_0 = QCz * v16_8_0 + WQz * v16_8_1 + (VT)1.0 * oo2e * (v16_2_0 - rho_e * v16_2_1);
-            const VT v17_18_0 = QCz * v17_8_0 + WQz * v17_8_1 + (VT)1.0 * oo2ze * v7_8_1 + (VT)1.0 * oo2e * (v17_2_0 - rho_e * v17_2_1);
-            const VT v18_18_0 = QCz * v18_8_0 + WQz * v18_8_1 + (VT)2.0 * oo2ze * v8_8_1 + (VT)1.0 * oo2e * (v18_2_0 - rho_e * v18_2_1);
-            const VT v19_18_0 = QCz * v19_8_0 + WQz * v19_8_1 + (VT)3.0 * oo2ze * v9_8_1 + (VT)1.0 * oo2e * (v19_2_0 - rho_e * v19_2_1);
-            const VT v4_19_0 = QCz * v4_9_0 + WQz * v4_9_1 + (VT)2.0 * oo2e * (v4_3_0 - rho_e * v4_3_1);
-            const VT v5_19_0 = QCz * v5_9_0 + WQz * v5_9_1 + (VT)2.0 * oo2e * (v5_3_0 - rho_e * v5_3_1);
-            const VT v6_19_0 = QCz * v6_9_0 + WQz * v6_9_1 + (VT)1.0 * oo2ze * v1_9_1 + (VT)2.0 * oo2e * (v6_3_0 - rho_e * v6_3_1);
-            const VT v7_19_0 = QCz * v7_9_0 + WQz * v7_9_1 + (VT)2.0 * oo2e * (v7_3_0 - rho_e * v7_3_1);
-            const VT v8_19_0 = QCz * v8_9_0 + WQz * v8_9_1 + (VT)1.0 * oo2ze * v2_9_1 + (VT)2.0 * oo2e * (v8_3_0 - rho_e * v8_3_1);
-            const VT v9_19_0 = QCz * v9_9_0 + WQz * v9_9_1 + (VT)2.0 * oo2ze * v3_9_1 + (VT)2.0 * oo2e * (v9_3_0 - rho_e * v9_3_1);
-            const VT v10_19_0 = QCz * v10_9_0 + WQz * v10_9_1 + (VT)2.0 * oo2e * (v10_3_0 - rho_e * v10_3_1);
-            const VT v11_19_0 = QCz * v11_9_0 + WQz * v11_9_1 + (VT)2.0 * oo2e * (v11_3_0 - rho_e * v11_3_1);
-            const VT v12_19_0 = QCz * v12_9_0 + WQz * v12_9_1 + (VT)1.0 * oo2ze * v4_9_1 + (VT)2.0 * oo2e * (v12_3_0 - rho_e * v12_3_1);
-            const VT v13_19_0 = QCz * v13_9_0 + WQz * v13_9_1 + (VT)2.0 * oo2e * (v13_3_0 - rho_e * v13_3_1);
-            const VT v14_19_0 = QCz * v14_9_0 + WQz * v14_9_1 + (VT)2.0 * oo2ze * v6_9_1 + (VT)2.0 * oo2e * (v14_3_0 - rho_e * v14_3_1);
-            const VT v15_19_0 = QCz * v15_9_0 + WQz * v15_9_1 + (VT)1.0 * oo2ze * v5_9_1 + (VT)2.0 * oo2e * (v15_3_0 - rho_e * v15_3_1);
-            const VT v16_19_0 = QCz * v16_9_0 + WQz * v16_9_1 + (VT)2.0 * oo2e * (v16_3_0 - rho_e * v16_3_1);
-            const VT v17_19_0 = QCz * v17_9_0 + WQz * v17_9_1 + (VT)1.0 * oo2ze * v7_9_1 + (VT)2.0 * oo2e * (v17_3_0 - rho_e * v17_3_1);
-            const VT v18_19_0 = QCz * v18_9_0 + WQz * v18_9_1 + (VT)2.0 * oo2ze * v8_9_1 + (VT)2.0 * oo2e * (v18_3_0 - rho_e * v18_3_1);
-            const VT v19_19_0 = QCz * v19_9_0 + WQz * v19_9_1 + (VT)3.0 * oo2ze * v9_9_1 + (VT)2.0 * oo2e * (v19_3_0 - rho_e * v19_3_1);
-            acc[0] += (double)v4_4_0;
-            acc[1] += (double)v4_5_0;
-            acc[2] += (double)v4_6_0;
-            acc[3] += (double)v4_7_0;
-            acc[4] += (double)v4_8_0;
-            acc[5] += (double)v4_9_0;
-            acc[6] += (double)v4_10_0;
-            acc[7] += (double)v4_11_0;
-            acc[8] += (double)v4_12_0;
-            acc[9] += (double)v4_13_0;
-            acc[10] += (double)v4_14_0;
-            acc[11] += (double)v4_15_0;
-            acc[12] += (double)v4_16_0;
-            acc[13] += (double)v4_17_0;
-            acc[14] += (double)v4_18_0;
-            acc[15] += (double)v4_19_0;
-            acc[16] += (double)v5_4_0;
-            acc[17] += (double)v5_5_0;
-            acc[18] += (double)v5_6_0;
-            acc[19] += (double)v5_7_0;
-            acc[20] += (double)v5_8_0;
-            acc[21] += (double)v5_9_0;
-            acc[22] += (double)v5_10_0;
-            acc[23] += (double)v5_11_0;
-            acc[24] += (double)v5_12_0;
-            acc[25] += (double)v5_13_0;
-            acc[26] += (double)v5_14_0;
-            acc[27] += (double)v5_15_0;
-            acc[28] += (double)v5_16_0;
-            acc[29] += (double)v5_17_0;
-            acc[30] += (double)v5_18_0;
-            acc[31] += (double)v5_19_0;
-            acc[32] += (double)v6_4_0;
-            acc[33] += (double)v6_5_0;
-            acc[34] += (double)v6_6_0;
-            acc[35] += (double)v6_7_0;
-            acc[36] += (double)v6_8_0;
-            acc[37] += (double)v6_9_0;
-            acc[38] += (double)v6_10_0;
-            acc[39] += (double)v6_11_0;
-            acc[40] += (double)v6_12_0;
-            acc[41] += (double)v6_13_0;
-            acc[42] += (double)v6_14_0;
-            acc[43] += (double)v6_15_0;
-            acc[44] += (double)v6_16_0;
-            acc[45] += (double)v6_17_0;
-            acc[46] += (double)v6_18_0;
-            acc[47] += (double)v6_19_0;
-            acc[48] += (double)v7_4_0;
-            acc[49] += (double)v7_5_0;
-            acc[50] += (double)v7_6_0;
-            acc[51] += (double)v7_7_0;
-            acc[52] += (double)v7_8_0;
-            acc[53] += (double)v7_9_0;
-            acc[54] += (double)v7_10_0;
-            acc[55] += (double)v7_11_0;
-            acc[56] += (double)v7_12_0;
-            acc[57] += (double)v7_13_0;
-            acc[58] += (double)v7_14_0;
-            acc[59] += (double)v7_15_0;
-            acc[60] += (double)v7_16_0;
-            acc[61] += (double)v7_17_0;
-            acc[62] += (double)v7_18_0;
-            acc[63] += (double)v7_19_0;
-            acc[64] += (double)v8_4_0;
-            acc[65] += (double)v8_5_0;
-            acc[66] += (double)v8_6_0;
-            acc[67] += (double)v8_7_0;
-            acc[68] += (double)v8_8_0;
-            acc[69] += (double)v8_9_0;
-            acc[70] += (double)v8_10_0;
-            acc[71] += (double)v8_11_0;
-            acc[72] += (double)v8_12_0;
-            acc[73] += (double)v8_13_0;
-            acc[74] += (double)v8_14_0;
-            acc[75] += (double)v8_15_0;
-            acc[76] += (double)v8_16_0;
-            acc[77] += (double)v8_17_0;
-            acc[78] += (double)v8_18_0;
-            acc[79] += (double)v8_19_0;
-            acc[80] += (double)v9_4_0;
-            acc[81] += (double)v9_5_0;
-            acc[82] += (double)v9_6_0;
-            acc[83] += (double)v9_7_0;
-            acc[84] += (double)v9_8_0;
-            acc[85] += (double)v9_9_0;
-            acc[86] += (double)v9_10_0;
-            acc[87] += (double)v9_11_0;
-            acc[88] += (double)v9_12_0;
-            acc[89] += (double)v9_13_0;
-            acc[90] += (double)v9_14_0;
-            acc[91] += (double)v9_15_0;
-            acc[92] += (double)v9_16_0;
-            acc[93] += (double)v9_17_0;
-            acc[94] += (double)v9_18_0;
-            acc[95] += (double)v9_19_0;
-            acc[96] += (double)v10_4_0;
-            acc[97] += (double)v10_5_0;
-            acc[98] += (double)v10_6_0;
-            acc[99] += (double)v10_7_0;
-            acc[100] += (double)v10_8_0;
-            acc[101] += (double)v10_9_0;
-            acc[102] += (double)v10_10_0;
-            acc[103] += (double)v10_11_0;
-            acc[104] += (double)v10_12_0;
-            acc[105] += (double)v10_13_0;
-            acc[106] += (double)v10_14_0;
-            acc[107] += (double)v10_15_0;
-            acc[108] += (double)v10_16_0;
-            acc[109] += (double)v10_17_0;
-            acc[110] += (double)v10_18_0;
-            acc[111] += (double)v10_19_0;
-            acc[112] += (double)v11_4_0;
-            acc[113] += (double)v11_5_0;
-            acc[114] += (double)v11_6_0;
-            acc[115] += (double)v11_7_0;
-            acc[116] += (double)v11_8_0;
-            acc[117] += (double)v11_9_0;
-            acc[118] += (double)v11_10_0;
-            acc[119] += (double)v11_11_0;
-            acc[120] += (double)v11_12_0;
-            acc[121] += (double)v11_13_0;
-            acc[122] += (double)v11_14_0;
-            acc[123] += (double)v11_15_0;
-            acc[124] += (double)v11_16_0;
-            acc[125] += (double)v11_17_0;
-            acc[126] += (double)v11_18_0;
-            acc[127] += (double)v11_19_0;
-            acc[128] += (double)v12_4_0;
-            acc[129] += (double)v12_5_0;
-            acc[130] += (double)v12_6_0;
-            acc[131] += (double)v12_7_0;
-            acc[132] += (double)v12_8_0;
-            acc[133] += (double)v12_9_0;
-            acc[134] += (double)v12_10_0;
-            acc[135] += (double)v12_11_0;
-            acc[136] += (double)v12_12_0;
-            acc[137] += (double)v12_13_0;
-            acc[138] += (double)v12_14_0;
-            acc[139] += (double)v12_15_0;
-            acc[140] += (double)v12_16_0;
-            acc[141] += (double)v12_17_0;
-            acc[142] += (double)v12_18_0;
-            acc[143] += (double)v12_19_0;
-            acc[144] += (double)v13_4_0;
-            acc[145] += (double)v13_5_0;
-            acc[146] += (double)v13_6_0;
-            acc[147] += (double)v13_7_0;
-            acc[148] += (double)v13_8_0;
-            acc[149] += (double)v13_9_0;
-            acc[150] += (double)v13_10_0;
-            acc[151] += (double)v13_11_0;
-            acc[152] += (double)v13_12_0;
-            acc[153] += (double)v13_13_0;
-            acc[154] += (double)v13_14_0;
-            acc[155] += (double)v13_15_0;
-            acc[156] += (double)v13_16_0;
-            acc[157] += (double)v13_17_0;
-            acc[158] += (double)v13_18_0;
-            acc[159] += (double)v13_19_0;
-            acc[160] += (double)v14_4_0;
-            acc[161] += (double)v14_5_0;
-            acc[162] += (double)v14_6_0;
-            acc[163] += (double)v14_7_0;
-            acc[164] += (double)v14_8_0;
-            acc[165] += (double)v14_9_0;
-            acc[166] += (double)v14_10_0;
-            acc[167] += (double)v14_11_0;
-            acc[168] += (double)v14_12_0;
-            acc[169] += (double)v14_13_0;
-            acc[170] += (double)v14_14_0;
-            acc[171] += (double)v14_15_0;
-            acc[172] += (double)v14_16_0;
-            acc[173] += (double)v14_17_0;
-            acc[174] += (double)v14_18_0;
-            acc[175] += (double)v14_19_0;
-            acc[176] += (double)v15_4_0;
-            acc[177] += (double)v15_5_0;
-            acc[178] += (double)v15_6_0;
-            acc[179] += (double)v15_7_0;
-            acc[180] += (double)v15_8_0;
-            acc[181] += (double)v15_9_0;
-            acc[182] += (double)v15_10_0;
-            acc[183] += (double)v15_11_0;
-            acc[184] += (double)v15_12_0;
-            acc[185] += (double)v15_13_0;
-            acc[186] += (double)v15_14_0;
-            acc[187] += (double)v15_15_0;
-            acc[188] += (double)v15_16_0;
-            acc[189] += (double)v15_17_0;
-            acc[190] += (double)v15_18_0;
-            acc[191] += (double)v15_19_0;
-            acc[192] += (double)v16_4_0;
-            acc[193] += (double)v16_5_0;
-            acc[194] += (double)v16_6_0;
-            acc[195] += (double)v16_7_0;
-            acc[196] += (double)v16_8_0;
-            acc[197] += (double)v16_9_0;
-            acc[198] += (double)v16_10_0;
-            acc[199] += (double)v16_11_0;
-            acc[200] += (double)v16_12_0;
-            acc[201] += (double)v16_13_0;
-            acc[202] += (double)v16_14_0;
-            acc[203] += (double)v16_15_0;
-            acc[204] += (double)v16_16_0;
-            acc[205] += (double)v16_17_0;
-            acc[206] += (double)v16_18_0;
-            acc[207] += (double)v16_19_0;
-            acc[208] += (double)v17_4_0;
-            acc[209] += (double)v17_5_0;
-            acc[210] += (double)v17_6_0;
-            acc[211] += (double)v17_7_0;
-            acc[212] += (double)v17_8_0;
-            acc[213] += (double)v17_9_0;
-            acc[214] += (double)v17_10_0;
-            acc[215] += (double)v17_11_0;
-            acc[216] += (double)v17_12_0;
-            acc[217] += (double)v17_13_0;
-            acc[218] += (double)v17_14_0;
-            acc[219] += (double)v17_15_0;
-            acc[220] += (double)v17_16_0;
-            acc[221] += (double)v17_17_0;
-            acc[222] += (double)v17_18_0;
-            acc[223] += (double)v17_19_0;
-            acc[224] += (double)v18_4_0;
-            acc[225] += (double)v18_5_0;
-            acc[226] += (double)v18_6_0;
-            acc[227] += (double)v18_7_0;
-            acc[228] += (double)v18_8_0;
-            acc[229] += (double)v18_9_0;
-            acc[230] += (double)v18_10_0;
-            acc[231] += (double)v18_11_0;
-            acc[232] += (double)v18_12_0;
-            acc[233] += (double)v18_13_0;
-            acc[234] += (double)v18_14_0;
-            acc[235] += (double)v18_15_0;
-            acc[236] += (double)v18_16_0;
-            acc[237] += (double)v18_17_0;
-            acc[238] += (double)v18_18_0;
-            acc[239] += (double)v18_19_0;
-            acc[240] += (double)v19_4_0;
-            acc[241] += (double)v19_5_0;
-            acc[242] += (double)v19_6_0;
-            acc[243] += (double)v19_7_0;
-            acc[244] += (double)v19_8_0;
-            acc[245] += (double)v19_9_0;
-            acc[246] += (double)v19_10_0;
-            acc[247] += (double)v19_11_0;
-            acc[248] += (double)v19_12_0;
-            acc[249] += (double)v19_13_0;
-            acc[250] += (double)v19_14_0;
-            acc[251] += (double)v19_15_0;
-            acc[252] += (double)v19_16_0;
-            acc[253] += (double)v19_17_0;
-            acc[254] += (double)v19_18_0;
-            acc[255] += (double)v19_19_0;
+            if constexpr (sizeof(VT) == 8) {
+                acc[0] += (double)v4_4_0;
+                acc[1] += (double)v4_5_0;
+                acc[2] += (double)v4_6_0;
+                acc[3] += (double)v4_7_0;
+                acc[4] += (double)v4_8_0;
+                acc[5] += (double)v4_9_0;
+                acc[6] = fma(QCx, v4_4_0, fma(WQx, v4_4_1, fma(2.0 * oo2ze, v1_4_1, fma(2.0 * oo2e, (v4_1_0 - rho_e * v4_1_1), acc[6]))));
+                acc[7] = fma(QCx, v4_5_0, fma(WQx, v4_5_1, fma(2.0 * oo2ze, v1_5_1, fma(1.0 * oo2e, (v4_2_0 - rho_e * v4_2_1), acc[7]))));
+                acc[8] = fma(QCx, v4_6_0, fma(WQx, v4_6_1, fma(2.0 * oo2ze, v1_6_1, fma(1.0 * oo2e, (v4_3_0 - rho_e * v4_3_1), acc[8]))));
+                acc[9] = fma(QCy, v4_5_0, fma(WQy, v4_5_1, fma(1.0 * oo2e, (v4_1_0 - rho_e * v4_1_1), acc[9])));
+                acc[10] = fma(QCz, v4_6_0, fma(WQz, v4_6_1, fma(1.0 * oo2e, (v4_1_0 - rho_e * v4_1_1), acc[10])));
+                acc[11] = fma(QCx, v4_8_0, fma(WQx, v4_8_1, fma(2.0 * oo2ze, v1_8_1, acc[11])));
+                acc[12] = fma(QCy, v4_7_0, fma(WQy, v4_7_1, fma(2.0 * oo2e, (v4_2_0 - rho_e * v4_2_1), acc[12])));
+                acc[13] = fma(QCy, v4_8_0, fma(WQy, v4_8_1, fma(1.0 * oo2e, (v4_3_0 - rho_e * v4_3_1), acc[13])));
+                acc[14] = fma(QCz, v4_8_0, fma(WQz, v4_8_1, fma(1.0 * oo2e, (v4_2_0 - rho_e * v4_2_1), acc[14])));
+                acc[15] = fma(QCz, v4_9_0, fma(WQz, v4_9_1, fma(2.0 * oo2e, (v4_3_0 - rho_e * v4_3_1), acc[15])));
+                acc[16] += (double)v5_4_0;
+                acc[17] += (double)v5_5_0;
+                acc[18] += (double)v5_6_0;
+                acc[19] += (double)v5_7_0;
+                acc[20] += (double)v5_8_0;
+                acc[21] += (double)v5_9_0;
+                acc[22] = fma(QCx, v5_4_0, fma(WQx, v5_4_1, fma(1.0 * oo2ze, v2_4_1, fma(2.0 * oo2e, (v5_1_0 - rho_e * v5_1_1), acc[22]))));
+                acc[23] = fma(QCx, v5_5_0, fma(WQx, v5_5_1, fma(1.0 * oo2ze, v2_5_1, fma(1.0 * oo2e, (v5_2_0 - rho_e * v5_2_1), acc[23]))));
+                acc[24] = fma(QCx, v5_6_0, fma(WQx, v5_6_1, fma(1.0 * oo2ze, v2_6_1, fma(1.0 * oo2e, (v5_3_0 - rho_e * v5_3_1), acc[24]))));
+                acc[25] = fma(QCy, v5_5_0, fma(WQy, v5_5_1, fma(1.0 * oo2ze, v1_5_1, fma(1.0 * oo2e, (v5_1_0 - rho_e * v5_1_1), acc[25]))));
+                acc[26] = fma(QCz, v5_6_0, fma(WQz, v5_6_1, fma(1.0 * oo2e, (v5_1_0 - rho_e * v5_1_1), acc[26])));
+                acc[27] = fma(QCx, v5_8_0, fma(WQx, v5_8_1, fma(1.0 * oo2ze, v2_8_1, acc[27])));
+                acc[28] = fma(QCy, v5_7_0, fma(WQy, v5_7_1, fma(1.0 * oo2ze, v1_7_1, fma(2.0 * oo2e, (v5_2_0 - rho_e * v5_2_1), acc[28]))));
+                acc[29] = fma(QCy, v5_8_0, fma(WQy, v5_8_1, fma(1.0 * oo2ze, v1_8_1, fma(1.0 * oo2e, (v5_3_0 - rho_e * v5_3_1), acc[29]))));
+                acc[30] = fma(QCz, v5_8_0, fma(WQz, v5_8_1, fma(1.0 * oo2e, (v5_2_0 - rho_e * v5_2_1), acc[30])));
+                acc[31] = fma(QCz, v5_9_0, fma(WQz, v5_9_1, fma(2.0 * oo2e, (v5_3_0 - rho_e * v5_3_1), acc[31])));
+                acc[32] += (double)v6_4_0;
+                acc[33] += (double)v6_5_0;
+                acc[34] += (double)v6_6_0;
+                acc[35] += (double)v6_7_0;
+                acc[36] += (double)v6_8_0;
+                acc[37] += (double)v6_9_0;
+                acc[38] = fma(QCx, v6_4_0, fma(WQx, v6_4_1, fma(1.0 * oo2ze, v3_4_1, fma(2.0 * oo2e, (v6_1_0 - rho_e * v6_1_1), acc[38]))));
+                acc[39] = fma(QCx, v6_5_0, fma(WQx, v6_5_1, fma(1.0 * oo2ze, v3_5_1, fma(1.0 * oo2e, (v6_2_0 - rho_e * v6_2_1), acc[39]))));
+                acc[40] = fma(QCx, v6_6_0, fma(WQx, v6_6_1, fma(1.0 * oo2ze, v3_6_1, fma(1.0 * oo2e, (v6_3_0 - rho_e * v6_3_1), acc[40]))));
+                acc[41] = fma(QCy, v6_5_0, fma(WQy, v6_5_1, fma(1.0 * oo2e, (v6_1_0 - rho_e * v6_1_1), acc[41])));
+                acc[42] = fma(QCz, v6_6_0, fma(WQz, v6_6_1, fma(1.0 * oo2ze, v1_6_1, fma(1.0 * oo2e, (v6_1_0 - rho_e * v6_1_1), acc[42]))));
+                acc[43] = fma(QCx, v6_8_0, fma(WQx, v6_8_1, fma(1.0 * oo2ze, v3_8_1, acc[43])));
+                acc[44] = fma(QCy, v6_7_0, fma(WQy, v6_7_1, fma(2.0 * oo2e, (v6_2_0 - rho_e * v6_2_1), acc[44])));
+                acc[45] = fma(QCy, v6_8_0, fma(WQy, v6_8_1, fma(1.0 * oo2e, (v6_3_0 - rho_e * v6_3_1), acc[45])));
+                acc[46] = fma(QCz, v6_8_0, fma(WQz, v6_8_1, fma(1.0 * oo2ze, v1_8_1, fma(1.0 * oo2e, (v6_2_0 - rho_e * v6_2_1), acc[46]))));
+                acc[47] = fma(QCz, v6_9_0, fma(WQz, v6_9_1, fma(1.0 * oo2ze, v1_9_1, fma(2.0 * oo2e, (v6_3_0 - rho_e * v6_3_1), acc[47]))));
+                acc[48] += (double)v7_4_0;
+                acc[49] += (double)v7_5_0;
+                acc[50] += (double)v7_6_0;
+                acc[51] += (double)v7_7_0;
+                acc[52] += (double)v7_8_0;
+                acc[53] += (double)v7_9_0;
+                acc[54] = fma(QCx, v7_4_0, fma(WQx, v7_4_1, fma(2.0 * oo2e, (v7_1_0 - rho_e * v7_1_1), acc[54])));
+                acc[55] = fma(QCx, v7_5_0, fma(WQx, v7_5_1, fma(1.0 * oo2e, (v7_2_0 - rho_e * v7_2_1), acc[55])));
+                acc[56] = fma(QCx, v7_6_0, fma(WQx, v7_6_1, fma(1.0 * oo2e, (v7_3_0 - rho_e * v7_3_1), acc[56])));
+                acc[57] = fma(QCy, v7_5_0, fma(WQy, v7_5_1, fma(2.0 * oo2ze, v2_5_1, fma(1.0 * oo2e, (v7_1_0 - rho_e * v7_1_1), acc[57]))));
+                acc[58] = fma(QCz, v7_6_0, fma(WQz, v7_6_1, fma(1.0 * oo2e, (v7_1_0 - rho_e * v7_1_1), acc[58])));
+                acc[59] = fma(QCx, v7_8_0, fma(WQx, v7_8_1, acc[59]));
+                acc[60] = fma(QCy, v7_7_0, fma(WQy, v7_7_1, fma(2.0 * oo2ze, v2_7_1, fma(2.0 * oo2e, (v7_2_0 - rho_e * v7_2_1), acc[60]))));
+                acc[61] = fma(QCy, v7_8_0, fma(WQy, v7_8_1, fma(2.0 * oo2ze, v2_8_1, fma(1.0 * oo2e, (v7_3_0 - rho_e * v7_3_1), acc[61]))));
+                acc[62] = fma(QCz, v7_8_0, fma(WQz, v7_8_1, fma(1.0 * oo2e, (v7_2_0 - rho_e * v7_2_1), acc[62])));
+                acc[63] = fma(QCz, v7_9_0, fma(WQz, v7_9_1, fma(2.0 * oo2e, (v7_3_0 - rho_e * v7_3_1), acc[63])));
+                acc[64] += (double)v8_4_0;
+                acc[65] += (double)v8_5_0;
+                acc[66] += (double)v8_6_0;
+                acc[67] += (double)v8_7_0;
+                acc[68] += (double)v8_8_0;
+                acc[69] += (double)v8_9_0;
+                acc[70] = fma(QCx, v8_4_0, fma(WQx, v8_4_1, fma(2.0 * oo2e, (v8_1_0 - rho_e * v8_1_1), acc[70])));
+                acc[71] = fma(QCx, v8_5_0, fma(WQx, v8_5_1, fma(1.0 * oo2e, (v8_2_0 - rho_e * v8_2_1), acc[71])));
+                acc[72] = fma(QCx, v8_6_0, fma(WQx, v8_6_1, fma(1.0 * oo2e, (v8_3_0 - rho_e * v8_3_1), acc[72])));
+                acc[73] = fma(QCy, v8_5_0, fma(WQy, v8_5_1, fma(1.0 * oo2ze, v3_5_1, fma(1.0 * oo2e, (v8_1_0 - rho_e * v8_1_1), acc[73]))));
+                acc[74] = fma(QCz, v8_6_0, fma(WQz, v8_6_1, fma(1.0 * oo2ze, v2_6_1, fma(1.0 * oo2e, (v8_1_0 - rho_e * v8_1_1), acc[74]))));
+                acc[75] = fma(QCx, v8_8_0, fma(WQx, v8_8_1, acc[75]));
+                acc[76] = fma(QCy, v8_7_0, fma(WQy, v8_7_1, fma(1.0 * oo2ze, v3_7_1, fma(2.0 * oo2e, (v8_2_0 - rho_e * v8_2_1), acc[76]))));
+                acc[77] = fma(QCy, v8_8_0, fma(WQy, v8_8_1, fma(1.0 * oo2ze, v3_8_1, fma(1.0 * oo2e, (v8_3_0 - rho_e * v8_3_1), acc[77]))));
+                acc[78] = fma(QCz, v8_8_0, fma(WQz, v8_8_1, fma(1.0 * oo2ze, v2_8_1, fma(1.0 * oo2e, (v8_2_0 - rho_e * v8_2_1), acc[78]))));
+                acc[79] = fma(QCz, v8_9_0, fma(WQz, v8_9_1, fma(1.0 * oo2ze, v2_9_1, fma(2.0 * oo2e, (v8_3_0 - rho_e * v8_3_1), acc[79]))));
+                acc[80] += (double)v9_4_0;
+                acc[81] += (double)v9_5_0;
+                acc[82] += (double)v9_6_0;
+                acc[83] += (double)v9_7_0;
+                acc[84] += (double)v9_8_0;
+                acc[85] += (double)v9_9_0;
+                acc[86] = fma(QCx, v9_4_0, fma(WQx, v9_4_1, fma(2.0 * oo2e, (v9_1_0 - rho_e * v9_1_1), acc[86])));
+                acc[87] = fma(QCx, v9_5_0, fma(WQx, v9_5_1, fma(1.0 * oo2e, (v9_2_0 - rho_e * v9_2_1), acc[87])));
+                acc[88] = fma(QCx, v9_6_0, fma(WQx, v9_6_1, fma(1.0 * oo2e, (v9_3_0 - rho_e * v9_3_1), acc[88])));
+                acc[89] = fma(QCy, v9_5_0, fma(WQy, v9_5_1, fma(1.0 * oo2e, (v9_1_0 - rho_e * v9_1_1), acc[89])));
+                acc[90] = fma(QCz, v9_6_0, fma(WQz, v9_6_1, fma(2.0 * oo2ze, v3_6_1, fma(1.0 * oo2e, (v9_1_0 - rho_e * v9_1_1), acc[90]))));
+                acc[91] = fma(QCx, v9_8_0, fma(WQx, v9_8_1, acc[91]));
+                acc[92] = fma(QCy, v9_7_0, fma(WQy, v9_7_1, fma(2.0 * oo2e, (v9_2_0 - rho_e * v9_2_1), acc[92])));
+                acc[93] = fma(QCy, v9_8_0, fma(WQy, v9_8_1, fma(1.0 * oo2e, (v9_3_0 - rho_e * v9_3_1), acc[93])));
+                acc[94] = fma(QCz, v9_8_0, fma(WQz, v9_8_1, fma(2.0 * oo2ze, v3_8_1, fma(1.0 * oo2e, (v9_2_0 - rho_e * v9_2_1), acc[94]))));
+                acc[95] = fma(QCz, v9_9_0, fma(WQz, v9_9_1, fma(2.0 * oo2ze, v3_9_1, fma(2.0 * oo2e, (v9_3_0 - rho_e * v9_3_1), acc[95]))));
+                acc[96] += (double)v10_4_0;
+                acc[97] += (double)v10_5_0;
+                acc[98] += (double)v10_6_0;
+                acc[99] += (double)v10_7_0;
+                acc[100] += (double)v10_8_0;
+                acc[101] += (double)v10_9_0;
+                acc[102] = fma(QCx, v10_4_0, fma(WQx, v10_4_1, fma(3.0 * oo2ze, v4_4_1, fma(2.0 * oo2e, (v10_1_0 - rho_e * v10_1_1), acc[102]))));
+                acc[103] = fma(QCx, v10_5_0, fma(WQx, v10_5_1, fma(3.0 * oo2ze, v4_5_1, fma(1.0 * oo2e, (v10_2_0 - rho_e * v10_2_1), acc[103]))));
+                acc[104] = fma(QCx, v10_6_0, fma(WQx, v10_6_1, fma(3.0 * oo2ze, v4_6_1, fma(1.0 * oo2e, (v10_3_0 - rho_e * v10_3_1), acc[104]))));
+                acc[105] = fma(QCy, v10_5_0, fma(WQy, v10_5_1, fma(1.0 * oo2e, (v10_1_0 - rho_e * v10_1_1), acc[105])));
+                acc[106] = fma(QCz, v10_6_0, fma(WQz, v10_6_1, fma(1.0 * oo2e, (v10_1_0 - rho_e * v10_1_1), acc[106])));
+                acc[107] = fma(QCx, v10_8_0, fma(WQx, v10_8_1, fma(3.0 * oo2ze, v4_8_1, acc[107])));
+                acc[108] = fma(QCy, v10_7_0, fma(WQy, v10_7_1, fma(2.0 * oo2e, (v10_2_0 - rho_e * v10_2_1), acc[108])));
+                acc[109] = fma(QCy, v10_8_0, fma(WQy, v10_8_1, fma(1.0 * oo2e, (v10_3_0 - rho_e * v10_3_1), acc[109])));
+                acc[110] = fma(QCz, v10_8_0, fma(WQz, v10_8_1, fma(1.0 * oo2e, (v10_2_0 - rho_e * v10_2_1), acc[110])));
+                acc[111] = fma(QCz, v10_9_0, fma(WQz, v10_9_1, fma(2.0 * oo2e, (v10_3_0 - rho_e * v10_3_1), acc[111])));
+                acc[112] += (double)v11_4_0;
+                acc[113] += (double)v11_5_0;
+                acc[114] += (double)v11_6_0;
+                acc[115] += (double)v11_7_0;
+                acc[116] += (double)v11_8_0;
+                acc[117] += (double)v11_9_0;
+                acc[118] = fma(QCx, v11_4_0, fma(WQx, v11_4_1, fma(2.0 * oo2ze, v5_4_1, fma(2.0 * oo2e, (v11_1_0 - rho_e * v11_1_1), acc[118]))));
+                acc[119] = fma(QCx, v11_5_0, fma(WQx, v11_5_1, fma(2.0 * oo2ze, v5_5_1, fma(1.0 * oo2e, (v11_2_0 - rho_e * v11_2_1), acc[119]))));
+                acc[120] = fma(QCx, v11_6_0, fma(WQx, v11_6_1, fma(2.0 * oo2ze, v5_6_1, fma(1.0 * oo2e, (v11_3_0 - rho_e * v11_3_1), acc[120]))));
+                acc[121] = fma(QCy, v11_5_0, fma(WQy, v11_5_1, fma(1.0 * oo2ze, v4_5_1, fma(1.0 * oo2e, (v11_1_0 - rho_e * v11_1_1), acc[121]))));
+                acc[122] = fma(QCz, v11_6_0, fma(WQz, v11_6_1, fma(1.0 * oo2e, (v11_1_0 - rho_e * v11_1_1), acc[122])));
+                acc[123] = fma(QCx, v11_8_0, fma(WQx, v11_8_1, fma(2.0 * oo2ze, v5_8_1, acc[123])));
+                acc[124] = fma(QCy, v11_7_0, fma(WQy, v11_7_1, fma(1.0 * oo2ze, v4_7_1, fma(2.0 * oo2e, (v11_2_0 - rho_e * v11_2_1), acc[124]))));
+                acc[125] = fma(QCy, v11_8_0, fma(WQy, v11_8_1, fma(1.0 * oo2ze, v4_8_1, fma(1.0 * oo2e, (v11_3_0 - rho_e * v11_3_1), acc[125]))));
+                acc[126] = fma(QCz, v11_8_0, fma(WQz, v11_8_1, fma(1.0 * oo2e, (v11_2_0 - rho_e * v11_2_1), acc[126])));
+                acc[127] = fma(QCz, v11_9_0, fma(WQz, v11_9_1, fma(2.0 * oo2e, (v11_3_0 - rho_e * v11_3_1), acc[127])));
+                acc[128] += (double)v12_4_0;
+                acc[129] += (double)v12_5_0;
+                acc[130] += (double)v12_6_0;
+                acc[131] += (double)v12_7_0;
+                acc[132] += (double)v12_8_0;
+                acc[133] += (double)v12_9_0;
+                acc[134] = fma(QCx, v12_4_0, fma(WQx, v12_4_1, fma(2.0 * oo2ze, v6_4_1, fma(2.0 * oo2e, (v12_1_0 - rho_e * v12_1_1), acc[134]))));
+                acc[135] = fma(QCx, v12_5_0, fma(WQx, v12_5_1, fma(2.0 * oo2ze, v6_5_1, fma(1.0 * oo2e, (v12_2_0 - rho_e * v12_2_1), acc[135]))));
+                acc[136] = fma(QCx, v12_6_0, fma(WQx, v12_6_1, fma(2.0 * oo2ze, v6_6_1, fma(1.0 * oo2e, (v12_3_0 - rho_e * v12_3_1), acc[136]))));
+                acc[137] = fma(QCy, v12_5_0, fma(WQy, v12_5_1, fma(1.0 * oo2e, (v12_1_0 - rho_e * v12_1_1), acc[137])));
+                acc[138] = fma(QCz, v12_6_0, fma(WQz, v12_6_1, fma(1.0 * oo2ze, v4_6_1, fma(1.0 * oo2e, (v12_1_0 - rho_e * v12_1_1), acc[138]))));
+                acc[139] = fma(QCx, v12_8_0, fma(WQx, v12_8_1, fma(2.0 * oo2ze, v6_8_1, acc[139])));
+                acc[140] = fma(QCy, v12_7_0, fma(WQy, v12_7_1, fma(2.0 * oo2e, (v12_2_0 - rho_e * v12_2_1), acc[140])));
+                acc[141] = fma(QCy, v12_8_0, fma(WQy, v12_8_1, fma(1.0 * oo2e, (v12_3_0 - rho_e * v12_3_1), acc[141])));
+                acc[142] = fma(QCz, v12_8_0, fma(WQz, v12_8_1, fma(1.0 * oo2ze, v4_8_1, fma(1.0 * oo2e, (v12_2_0 - rho_e * v12_2_1), acc[142]))));
+                acc[143] = fma(QCz, v12_9_0, fma(WQz, v12_9_1, fma(1.0 * oo2ze, v4_9_1, fma(2.0 * oo2e, (v12_3_0 - rho_e * v12_3_1), acc[143]))));
+                acc[144] += (double)v13_4_0;
+                acc[145] += (double)v13_5_0;
+                acc[146] += (double)v13_6_0;
+                acc[147] += (double)v13_7_0;
+                acc[148] += (double)v13_8_0;
+                acc[149] += (double)v13_9_0;
+                acc[150] = fma(QCx, v13_4_0, fma(WQx, v13_4_1, fma(1.0 * oo2ze, v7_4_1, fma(2.0 * oo2e, (v13_1_0 - rho_e * v13_1_1), acc[150]))));
+                acc[151] = fma(QCx, v13_5_0, fma(WQx, v13_5_1, fma(1.0 * oo2ze, v7_5_1, fma(1.0 * oo2e, (v13_2_0 - rho_e * v13_2_1), acc[151]))));
+                acc[152] = fma(QCx, v13_6_0, fma(WQx, v13_6_1, fma(1.0 * oo2ze, v7_6_1, fma(1.0 * oo2e, (v13_3_0 - rho_e * v13_3_1), acc[152]))));
+                acc[153] = fma(QCy, v13_5_0, fma(WQy, v13_5_1, fma(2.0 * oo2ze, v5_5_1, fma(1.0 * oo2e, (v13_1_0 - rho_e * v13_1_1), acc[153]))));
+                acc[154] = fma(QCz, v13_6_0, fma(WQz, v13_6_1, fma(1.0 * oo2e, (v13_1_0 - rho_e * v13_1_1), acc[154])));
+                acc[155] = fma(QCx, v13_8_0, fma(WQx, v13_8_1, fma(1.0 * oo2ze, v7_8_1, acc[155])));
+                acc[156] = fma(QCy, v13_7_0, fma(WQy, v13_7_1, fma(2.0 * oo2ze, v5_7_1, fma(2.0 * oo2e, (v13_2_0 - rho_e * v13_2_1), acc[156]))));
+                acc[157] = fma(QCy, v13_8_0, fma(WQy, v13_8_1, fma(2.0 * oo2ze, v5_8_1, fma(1.0 * oo2e, (v13_3_0 - rho_e * v13_3_1), acc[157]))));
+                acc[158] = fma(QCz, v13_8_0, fma(WQz, v13_8_1, fma(1.0 * oo2e, (v13_2_0 - rho_e * v13_2_1), acc[158])));
+                acc[159] = fma(QCz, v13_9_0, fma(WQz, v13_9_1, fma(2.0 * oo2e, (v13_3_0 - rho_e * v13_3_1), acc[159])));
+                acc[160] += (double)v14_4_0;
+                acc[161] += (double)v14_5_0;
+                acc[162] += (double)v14_6_0;
+                acc[163] += (double)v14_7_0;
+                acc[164] += (double)v14_8_0;
+                acc[165] += (double)v14_9_0;
+                acc[166] = fma(QCx, v14_4_0, fma(WQx, v14_4_1, fma(1.0 * oo2ze, v9_4_1, fma(2.0 * oo2e, (v14_1_0 - rho_e * v14_1_1), acc[166]))));
+                acc[167] = fma(QCx, v14_5_0, fma(WQx, v14_5_1, fma(1.0 * oo2ze, v9_5_1, fma(1.0 * oo2e, (v14_2_0 - rho_e * v14_2_1), acc[167]))));
+                acc[168] = fma(QCx, v14_6_0, fma(WQx, v14_6_1, fma(1.0 * oo2ze, v9_6_1, fma(1.0 * oo2e, (v14_3_0 - rho_e * v14_3_1), acc[168]))));
+                acc[169] = fma(QCy, v14_5_0, fma(WQy, v14_5_1, fma(1.0 * oo2e, (v14_1_0 - rho_e * v14_1_1), acc[169])));
+                acc[170] = fma(QCz, v14_6_0, fma(WQz, v14_6_1, fma(2.0 * oo2ze, v6_6_1, fma(1.0 * oo2e, (v14_1_0 - rho_e * v14_1_1), acc[170]))));
+                acc[171] = fma(QCx, v14_8_0, fma(WQx, v14_8_1, fma(1.0 * oo2ze, v9_8_1, acc[171])));
+                acc[172] = fma(QCy, v14_7_0, fma(WQy, v14_7_1, fma(2.0 * oo2e, (v14_2_0 - rho_e * v14_2_1), acc[172])));
+                acc[173] = fma(QCy, v14_8_0, fma(WQy, v14_8_1, fma(1.0 * oo2e, (v14_3_0 - rho_e * v14_3_1), acc[173])));
+                acc[174] = fma(QCz, v14_8_0, fma(WQz, v14_8_1, fma(2.0 * oo2ze, v6_8_1, fma(1.0 * oo2e, (v14_2_0 - rho_e * v14_2_1), acc[174]))));
+                acc[175] = fma(QCz, v14_9_0, fma(WQz, v14_9_1, fma(2.0 * oo2ze, v6_9_1, fma(2.0 * oo2e, (v14_3_0 - rho_e * v14_3_1), acc[175]))));
+                acc[176] += (double)v15_4_0;
+                acc[177] += (double)v15_5_0;
+                acc[178] += (double)v15_6_0;
+                acc[179] += (double)v15_7_0;
+                acc[180] += (double)v15_8_0;
+                acc[181] += (double)v15_9_0;
+                acc[182] = fma(QCx, v15_4_0, fma(WQx, v15_4_1, fma(1.0 * oo2ze, v8_4_1, fma(2.0 * oo2e, (v15_1_0 - rho_e * v15_1_1), acc[182]))));
+                acc[183] = fma(QCx, v15_5_0, fma(WQx, v15_5_1, fma(1.0 * oo2ze, v8_5_1, fma(1.0 * oo2e, (v15_2_0 - rho_e * v15_2_1), acc[183]))));
+                acc[184] = fma(QCx, v15_6_0, fma(WQx, v15_6_1, fma(1.0 * oo2ze, v8_6_1, fma(1.0 * oo2e, (v15_3_0 - rho_e * v15_3_1), acc[184]))));
+                acc[185] = fma(QCy, v15_5_0, fma(WQy, v15_5_1, fma(1.0 * oo2ze, v6_5_1, fma(1.0 * oo2e, (v15_1_0 - rho_e * v15_1_1), acc[185]))));
+                acc[186] = fma(QCz, v15_6_0, fma(WQz, v15_6_1, fma(1.0 * oo2ze, v5_6_1, fma(1.0 * oo2e, (v15_1_0 - rho_e * v15_1_1), acc[186]))));
+                acc[187] = fma(QCx, v15_8_0, fma(WQx, v15_8_1, fma(1.0 * oo2ze, v8_8_1, acc[187])));
+                acc[188] = fma(QCy, v15_7_0, fma(WQy, v15_7_1, fma(1.0 * oo2ze, v6_7_1, fma(2.0 * oo2e, (v15_2_0 - rho_e * v15_2_1), acc[188]))));
+                acc[189] = fma(QCy, v15_8_0, fma(WQy, v15_8_1, fma(1.0 * oo2ze, v6_8_1, fma(1.0 * oo2e, (v15_3_0 - rho_e * v15_3_1), acc[189]))));
+                acc[190] = fma(QCz, v15_8_0, fma(WQz, v15_8_1, fma(1.0 * oo2ze, v5_8_1, fma(1.0 * oo2e, (v15_2_0 - rho_e * v15_2_1), acc[190]))));
+                acc[191] = fma(QCz, v15_9_0, fma(WQz, v15_9_1, fma(1.0 * oo2ze, v5_9_1, fma(2.0 * oo2e, (v15_3_0 - rho_e * v15_3_1), acc[191]))));
+                acc[192] += (double)v16_4_0;
+                acc[193] += (double)v16_5_0;
+                acc[194] += (double)v16_6_0;
+                acc[195] += (double)v16_7_0;
+                acc[196] += (double)v16_8_0;
+                acc[197] += (double)v16_9_0;
+                acc[198] = fma(QCx, v16_4_0, fma(WQx, v16_4_1, fma(2.0 * oo2e, (v16_1_0 - rho_e * v16_1_1), acc[198])));
+                acc[199] = fma(QCx, v16_5_0, fma(WQx, v16_5_1, fma(1.0 * oo2e, (v16_2_0 - rho_e * v16_2_1), acc[199])));
+                acc[200] = fma(QCx, v16_6_0, fma(WQx, v16_6_1, fma(1.0 * oo2e, (v16_3_0 - rho_e * v16_3_1), acc[200])));
+                acc[201] = fma(QCy, v16_5_0, fma(WQy, v16_5_1, fma(3.0 * oo2ze, v7_5_1, fma(1.0 * oo2e, (v16_1_0 - rho_e * v16_1_1), acc[201]))));
+                acc[202] = fma(QCz, v16_6_0, fma(WQz, v16_6_1, fma(1.0 * oo2e, (v16_1_0 - rho_e * v16_1_1), acc[202])));
+                acc[203] = fma(QCx, v16_8_0, fma(WQx, v16_8_1, acc[203]));
+                acc[204] = fma(QCy, v16_7_0, fma(WQy, v16_7_1, fma(3.0 * oo2ze, v7_7_1, fma(2.0 * oo2e, (v16_2_0 - rho_e * v16_2_1), acc[204]))));
+                acc[205] = fma(QCy, v16_8_0, fma(WQy, v16_8_1, fma(3.0 * oo2ze, v7_8_1, fma(1.0 * oo2e, (v16_3_0 - rho_e * v16_3_1), acc[205]))));
+                acc[206] = fma(QCz, v16_8_0, fma(WQz, v16_8_1, fma(1.0 * oo2e, (v16_2_0 - rho_e * v16_2_1), acc[206])));
+                acc[207] = fma(QCz, v16_9_0, fma(WQz, v16_9_1, fma(2.0 * oo2e, (v16_3_0 - rho_e * v16_3_1), acc[207])));
+                acc[208] += (double)v17_4_0;
+                acc[209] += (double)v17_5_0;
+                acc[210] += (double)v17_6_0;
+                acc[211] += (double)v17_7_0;
+                acc[212] += (double)v17_8_0;
+                acc[213] += (double)v17_9_0;
+                acc[214] = fma(QCx, v17_4_0, fma(WQx, v17_4_1, fma(2.0 * oo2e, (v17_1_0 - rho_e * v17_1_1), acc[214])));
+                acc[215] = fma(QCx, v17_5_0, fma(WQx, v17_5_1, fma(1.0 * oo2e, (v17_2_0 - rho_e * v17_2_1), acc[215])));
+                acc[216] = fma(QCx, v17_6_0, fma(WQx, v17_6_1, fma(1.0 * oo2e, (v17_3_0 - rho_e * v17_3_1), acc[216])));
+                acc[217] = fma(QCy, v17_5_0, fma(WQy, v17_5_1, fma(2.0 * oo2ze, v8_5_1, fma(1.0 * oo2e, (v17_1_0 - rho_e * v17_1_1), acc[217]))));
+                acc[218] = fma(QCz, v17_6_0, fma(WQz, v17_6_1, fma(1.0 * oo2ze, v7_6_1, fma(1.0 * oo2e, (v17_1_0 - rho_e * v17_1_1), acc[218]))));
+                acc[219] = fma(QCx, v17_8_0, fma(WQx, v17_8_1, acc[219]));
+                acc[220] = fma(QCy, v17_7_0, fma(WQy, v17_7_1, fma(2.0 * oo2ze, v8_7_1, fma(2.0 * oo2e, (v17_2_0 - rho_e * v17_2_1), acc[220]))));
+                acc[221] = fma(QCy, v17_8_0, fma(WQy, v17_8_1, fma(2.0 * oo2ze, v8_8_1, fma(1.0 * oo2e, (v17_3_0 - rho_e * v17_3_1), acc[221]))));
+                acc[222] = fma(QCz, v17_8_0, fma(WQz, v17_8_1, fma(1.0 * oo2ze, v7_8_1, fma(1.0 * oo2e, (v17_2_0 - rho_e * v17_2_1), acc[222]))));
+                acc[223] = fma(QCz, v17_9_0, fma(WQz, v17_9_1, fma(1.0 * oo2ze, v7_9_1, fma(2.0 * oo2e, (v17_3_0 - rho_e * v17_3_1), acc[223]))));
+                acc[224] += (double)v18_4_0;
+                acc[225] += (double)v18_5_0;
+                acc[226] += (double)v18_6_0;
+                acc[227] += (double)v18_7_0;
+                acc[228] += (double)v18_8_0;
+                acc[229] += (double)v18_9_0;
+                acc[230] = fma(QCx, v18_4_0, fma(WQx, v18_4_1, fma(2.0 * oo2e, (v18_1_0 - rho_e * v18_1_1), acc[230])));
+                acc[231] = fma(QCx, v18_5_0, fma(WQx, v18_5_1, fma(1.0 * oo2e, (v18_2_0 - rho_e * v18_2_1), acc[231])));
+                acc[232] = fma(QCx, v18_6_0, fma(WQx, v18_6_1, fma(1.0 * oo2e, (v18_3_0 - rho_e * v18_3_1), acc[232])));
+                acc[233] = fma(QCy, v18_5_0, fma(WQy, v18_5_1, fma(1.0 * oo2ze, v9_5_1, fma(1.0 * oo2e, (v18_1_0 - rho_e * v18_1_1), acc[233]))));
+                acc[234] = fma(QCz, v18_6_0, fma(WQz, v18_6_1, fma(2.0 * oo2ze, v8_6_1, fma(1.0 * oo2e, (v18_1_0 - rho_e * v18_1_1), acc[234]))));
+                acc[235] = fma(QCx, v18_8_0, fma(WQx, v18_8_1, acc[235]));
+                acc[236] = fma(QCy, v18_7_0, fma(WQy, v18_7_1, fma(1.0 * oo2ze, v9_7_1, fma(2.0 * oo2e, (v18_2_0 - rho_e * v18_2_1), acc[236]))));
+                acc[237] = fma(QCy, v18_8_0, fma(WQy, v18_8_1, fma(1.0 * oo2ze, v9_8_1, fma(1.0 * oo2e, (v18_3_0 - rho_e * v18_3_1), acc[237]))));
+                acc[238] = fma(QCz, v18_8_0, fma(WQz, v18_8_1, fma(2.0 * oo2ze, v8_8_1, fma(1.0 * oo2e, (v18_2_0 - rho_e * v18_2_1), acc[238]))));
+                acc[239] = fma(QCz, v18_9_0, fma(WQz, v18_9_1, fma(2.0 * oo2ze, v8_9_1, fma(2.0 * oo2e, (v18_3_0 - rho_e * v18_3_1), acc[239]))));
+                acc[240] += (double)v19_4_0;
+                acc[241] += (double)v19_5_0;
+                acc[242] += (double)v19_6_0;
+                acc[243] += (double)v19_7_0;
+                acc[244] += (double)v19_8_0;
+                acc[245] += (double)v19_9_0;
+                acc[246] = fma(QCx, v19_4_0, fma(WQx, v19_4_1, fma(2.0 * oo2e, (v19_1_0 - rho_e * v19_1_1), acc[246])));
+                acc[247] = fma(QCx, v19_5_0, fma(WQx, v19_5_1, fma(1.0 * oo2e, (v19_2_0 - rho_e * v19_2_1), acc[247])));
+                acc[248] = fma(QCx, v19_6_0, fma(WQx, v19_6_1, fma(1.0 * oo2e, (v19_3_0 - rho_e * v19_3_1), acc[248])));
+                acc[249] = fma(QCy, v19_5_0, fma(WQy, v19_5_1, fma(1.0 * oo2e, (v19_1_0 - rho_e * v19_1_1), acc[249])));
+                acc[250] = fma(QCz, v19_6_0, fma(WQz, v19_6_1, fma(3.0 * oo2ze, v9_6_1, fma(1.0 * oo2e, (v19_1_0 - rho_e * v19_1_1), acc[250]))));
+                acc[251] = fma(QCx, v19_8_0, fma(WQx, v19_8_1, acc[251]));
+                acc[252] = fma(QCy, v19_7_0, fma(WQy, v19_7_1, fma(2.0 * oo2e, (v19_2_0 - rho_e * v19_2_1), acc[252])));
+                acc[253] = fma(QCy, v19_8_0, fma(WQy, v19_8_1, fma(1.0 * oo2e, (v19_3_0 - rho_e * v19_3_1), acc[253])));
+                acc[254] = fma(QCz, v19_8_0, fma(WQz, v19_8_1, fma(3.0 * oo2ze, v9_8_1, fma(1.0 * oo2e, (v19_2_0 - rho_e * v19_2_1), acc[254]))));
+                acc[255] = fma(QCz, v19_9_0, fma(WQz, v19_9_1, fma(3.0 * oo2ze, v9_9_1, fma(2.0 * oo2e, (v19_3_0 - rho_e * v19_3_1), acc[255]))));
+            } else {
+                acc[0] += (double)v4_4_0;
+                acc[1] += (double)v4_5_0;
+                acc[2] += (double)v4_6_0;
+                acc[3] += (double)v4_7_0;
+                acc[4] += (double)v4_8_0;
+                acc[5] += (double)v4_9_0;
+                const VT v4_10_0 = QCx * v4_4_0 + WQx * v4_4_1 + (VT)2.0 * oo2ze * v1_4_1 + (VT)2.0 * oo2e * (v4_1_0 - rho_e * v4_1_1);
+                acc[6] += (double)v4_10_0;
+                const VT v4_11_0 = QCx * v4_5_0 + WQx * v4_5_1 + (VT)2.0 * oo2ze * v1_5_1 + (VT)1.0 * oo2e * (v4_2_0 - rho_e * v4_2_1);
+                acc[7] += (double)v4_11_0;
+                const VT v4_12_0 = QCx * v4_6_0 + WQx * v4_6_1 + (VT)2.0 * oo2ze * v1_6_1 + (VT)1.0 * oo2e * (v4_3_0 - rho_e * v4_3_1);
+                acc[8] += (double)v4_12_0;
+                const VT v4_13_0 = QCy * v4_5_0 + WQy * v4_5_1 + (VT)1.0 * oo2e * (v4_1_0 - rho_e * v4_1_1);
+                acc[9] += (double)v4_13_0;
+                const VT v4_14_0 = QCz * v4_6_0 + WQz * v4_6_1 + (VT)1.0 * oo2e * (v4_1_0 - rho_e * v4_1_1);
+                acc[10] += (double)v4_14_0;
+                const VT v4_15_0 = QCx * v4_8_0 + WQx * v4_8_1 + (VT)2.0 * oo2ze * v1_8_1;
+                acc[11] += (double)v4_15_0;
+                const VT v4_16_0 = QCy * v4_7_0 + WQy * v4_7_1 + (VT)2.0 * oo2e * (v4_2_0 - rho_e * v4_2_1);
+                acc[12] += (double)v4_16_0;
+                const VT v4_17_0 = QCy * v4_8_0 + WQy * v4_8_1 + (VT)1.0 * oo2e * (v4_3_0 - rho_e * v4_3_1);
+                acc[13] += (double)v4_17_0;
+                const VT v4_18_0 = QCz * v4_8_0 + WQz * v4_8_1 + (VT)1.0 * oo2e * (v4_2_0 - rho_e * v4_2_1);
+                acc[14] += (double)v4_18_0;
+                const VT v4_19_0 = QCz * v4_9_0 + WQz * v4_9_1 + (VT)2.0 * oo2e * (v4_3_0 - rho_e * v4_3_1);
+                acc[15] += (double)v4_19_0;
+                acc[16] += (double)v5_4_0;
+                acc[17] += (double)v5_5_0;
+                acc[18] += (double)v5_6_0;
+                acc[19] += (double)v5_7_0;
+                acc[20] += (double)v5_8_0;
+                acc[21] += (double)v5_9_0;
+                const VT v5_10_0 = QCx * v5_4_0 + WQx * v5_4_1 + (VT)1.0 * oo2ze * v2_4_1 + (VT)2.0 * oo2e * (v5_1_0 - rho_e * v5_1_1);
+                acc[22] += (double)v5_10_0;
+                const VT v5_11_0 = QCx * v5_5_0 + WQx * v5_5_1 + (VT)1.0 * oo2ze * v2_5_1 + (VT)1.0 * oo2e * (v5_2_0 - rho_e * v5_2_1);
+                acc[23] += (double)v5_11_0;
+                const VT v5_12_0 = QCx * v5_6_0 + WQx * v5_6_1 + (VT)1.0 * oo2ze * v2_6_1 + (VT)1.0 * oo2e * (v5_3_0 - rho_e * v5_3_1);
+                acc[24] += (double)v5_12_0;
+                const VT v5_13_0 = QCy * v5_5_0 + WQy * v5_5_1 + (VT)1.0 * oo2ze * v1_5_1 + (VT)1.0 * oo2e * (v5_1_0 - rho_e * v5_1_1);
+                acc[25] += (double)v5_13_0;
+                const VT v5_14_0 = QCz * v5_6_0 + WQz * v5_6_1 + (VT)1.0 * oo2e * (v5_1_0 - rho_e * v5_1_1);
+                acc[26] += (double)v5_14_0;
+                const VT v5_15_0 = QCx * v5_8_0 + WQx * v5_8_1 + (VT)1.0 * oo2ze * v2_8_1;
+                acc[27] += (double)v5_15_0;
+                const VT v5_16_0 = QCy * v5_7_0 + WQy * v5_7_1 + (VT)1.0 * oo2ze * v1_7_1 + (VT)2.0 * oo2e * (v5_2_0 - rho_e * v5_2_1);
+                acc[28] += (double)v5_16_0;
+                const VT v5_17_0 = QCy * v5_8_0 + WQy * v5_8_1 + (VT)1.0 * oo2ze * v1_8_1 + (VT)1.0 * oo2e * (v5_3_0 - rho_e * v5_3_1);
+                acc[29] += (double)v5_17_0;
+                const VT v5_18_0 = QCz * v5_8_0 + WQz * v5_8_1 + (VT)1.0 * oo2e * (v5_2_0 - rho_e * v5_2_1);
+                acc[30] += (double)v5_18_0;
+                const VT v5_19_0 = QCz * v5_9_0 + WQz * v5_9_1 + (VT)2.0 * oo2e * (v5_3_0 - rho_e * v5_3_1);
+                acc[31] += (double)v5_19_0;
+                acc[32] += (double)v6_4_0;
+                acc[33] += (double)v6_5_0;
+                acc[34] += (double)v6_6_0;
+                acc[35] += (double)v6_7_0;
+                acc[36] += (double)v6_8_0;
+                acc[37] += (double)v6_9_0;
+                const VT v6_10_0 = QCx * v6_4_0 + WQx * v6_4_1 + (VT)1.0 * oo2ze * v3_4_1 + (VT)2.0 * oo2e * (v6_1_0 - rho_e * v6_1_1);
+                acc[38] += (double)v6_10_0;
+                const VT v6_11_0 = QCx * v6_5_0 + WQx * v6_5_1 + (VT)1.0 * oo2ze * v3_5_1 + (VT)1.0 * oo2e * (v6_2_0 - rho_e * v6_2_1);
+                acc[39] += (double)v6_11_0;
+                const VT v6_12_0 = QCx * v6_6_0 + WQx * v6_6_1 + (VT)1.0 * oo2ze * v3_6_1 + (VT)1.0 * oo2e * (v6_3_0 - rho_e * v6_3_1);
+                acc[40] += (double)v6_12_0;
+                const VT v6_13_0 = QCy * v6_5_0 + WQy * v6_5_1 + (VT)1.0 * oo2e * (v6_1_0 - rho_e * v6_1_1);
+                acc[41] += (double)v6_13_0;
+                const VT v6_14_0 = QCz * v6_6_0 + WQz * v6_6_1 + (VT)1.0 * oo2ze * v1_6_1 + (VT)1.0 * oo2e * (v6_1_0 - rho_e * v6_1_1);
+                acc[42] += (double)v6_14_0;
+                const VT v6_15_0 = QCx * v6_8_0 + WQx * v6_8_1 + (VT)1.0 * oo2ze * v3_8_1;
+                acc[43] += (double)v6_15_0;
+                const VT v6_16_0 = QCy * v6_7_0 + WQy * v6_7_1 + (VT)2.0 * oo2e * (v6_2_0 - rho_e * v6_2_1);
+                acc[44] += (double)v6_16_0;
+                const VT v6_17_0 = QCy * v6_8_0 + WQy * v6_8_1 + (VT)1.0 * oo2e * (v6_3_0 - rho_e * v6_3_1);
+                acc[45] += (double)v6_17_0;
+                const VT v6_18_0 = QCz * v6_8_0 + WQz * v6_8_1 + (VT)1.0 * oo2ze * v1_8_1 + (VT)1.0 * oo2e * (v6_2_0 - rho_e * v6_2_1);
+                acc[46] += (double)v6_18_0;
+                const VT v6_19_0 = QCz * v6_9_0 + WQz * v6_9_1 + (VT)1.0 * oo2ze * v1_9_1 + (VT)2.0 * oo2e * (v6_3_0 - rho_e * v6_3_1);
+                acc[47] += (double)v6_19_0;
+                acc[48] += (double)v7_4_0;
+                acc[49] += (double)v7_5_0;
+                acc[50] += (double)v7_6_0;
+                acc[51] += (double)v7_7_0;
+                acc[52] += (double)v7_8_0;
+                acc[53] += (double)v7_9_0;
+                const VT v7_10_0 = QCx * v7_4_0 + WQx * v7_4_1 + (VT)2.0 * oo2e * (v7_1_0 - rho_e * v7_1_1);
+                acc[54] += (double)v7_10_0;
+                const VT v7_11_0 = QCx * v7_5_0 + WQx * v7_5_1 + (VT)1.0 * oo2e * (v7_2_0 - rho_e * v7_2_1);
+                acc[55] += (double)v7_11_0;
+                const VT v7_12_0 = QCx * v7_6_0 + WQx * v7_6_1 + (VT)1.0 * oo2e * (v7_3_0 - rho_e * v7_3_1);
+                acc[56] += (double)v7_12_0;
+                const VT v7_13_0 = QCy * v7_5_0 + WQy * v7_5_1 + (VT)2.0 * oo2ze * v2_5_1 + (VT)1.0 * oo2e * (v7_1_0 - rho_e * v7_1_1);
+                acc[57] += (double)v7_13_0;
+                const VT v7_14_0 = QCz * v7_6_0 + WQz * v7_6_1 + (VT)1.0 * oo2e * (v7_1_0 - rho_e * v7_1_1);
+                acc[58] += (double)v7_14_0;
+                const VT v7_15_0 = QCx * v7_8_0 + WQx * v7_8_1;
+                acc[59] += (double)v7_15_0;
+                const VT v7_16_0 = QCy * v7_7_0 + WQy * v7_7_1 + (VT)2.0 * oo2ze * v2_7_1 + (VT)2.0 * oo2e * (v7_2_0 - rho_e * v7_2_1);
+                acc[60] += (double)v7_16_0;
+                const VT v7_17_0 = QCy * v7_8_0 + WQy * v7_8_1 + (VT)2.0 * oo2ze * v2_8_1 + (VT)1.0 * oo2e * (v7_3_0 - rho_e * v7_3_1);
+                acc[61] += (double)v7_17_0;
+                const VT v7_18_0 = QCz * v7_8_0 + WQz * v7_8_1 + (VT)1.0 * oo2e * (v7_2_0 - rho_e * v7_2_1);
+                acc[62] += (double)v7_18_0;
+                const VT v7_19_0 = QCz * v7_9_0 + WQz * v7_9_1 + (VT)2.0 * oo2e * (v7_3_0 - rho_e * v7_3_1);
+                acc[63] += (double)v7_19_0;
+                acc[64] += (double)v8_4_0;
+                acc[65] += (double)v8_5_0;
+                acc[66] += (double)v8_6_0;
+                acc[67] += (double)v8_7_0;
+                acc[68] += (double)v8_8_0;
+                acc[69] += (double)v8_9_0;
+                const VT v8_10_0 = QCx * v8_4_0 + WQx * v8_4_1 + (VT)2.0 * oo2e * (v8_1_0 - rho_e * v8_1_1);
+                acc[70] += (double)v8_10_0;
+                const VT v8_11_0 = QCx * v8_5_0 + WQx * v8_5_1 + (VT)1.0 * oo2e * (v8_2_0 - rho_e * v8_2_1);
+                acc[71] += (double)v8_11_0;
+                const VT v8_12_0 = QCx * v8_6_0 + WQx * v8_6_1 + (VT)1.0 * oo2e * (v8_3_0 - rho_e * v8_3_1);
+                acc[72] += (double)v8_12_0;
+                const VT v8_13_0 = QCy * v8_5_0 + WQy * v8_5_1 + (VT)1.0 * oo2ze * v3_5_1 + (VT)1.0 * oo2e * (v8_1_0 - rho_e * v8_1_1);
+                acc[73] += (double)v8_13_0;
+                const VT v8_14_0 = QCz * v8_6_0 + WQz * v8_6_1 + (VT)1.0 * oo2ze * v2_6_1 + (VT)1.0 * oo2e * (v8_1_0 - rho_e * v8_1_1);
+                acc[74] += (double)v8_14_0;
+                const VT v8_15_0 = QCx * v8_8_0 + WQx * v8_8_1;
+                acc[75] += (double)v8_15_0;
+                const VT v8_16_0 = QCy * v8_7_0 + WQy * v8_7_1 + (VT)1.0 * oo2ze * v3_7_1 + (VT)2.0 * oo2e * (v8_2_0 - rho_e * v8_2_1);
+                acc[76] += (double)v8_16_0;
+                const VT v8_17_0 = QCy * v8_8_0 + WQy * v8_8_1 + (VT)1.0 * oo2ze * v3_8_1 + (VT)1.0 * oo2e * (v8_3_0 - rho_e * v8_3_1);
+                acc[77] += (double)v8_17_0;
+                const VT v8_18_0 = QCz * v8_8_0 + WQz * v8_8_1 + (VT)1.0 * oo2ze * v2_8_1 + (VT)1.0 * oo2e * (v8_2_0 - rho_e * v8_2_1);
+                acc[78] += (double)v8_18_0;
+                const VT v8_19_0 = QCz * v8_9_0 + WQz * v8_9_1 + (VT)1.0 * oo2ze * v2_9_1 + (VT)2.0 * oo2e * (v8_3_0 - rho_e * v8_3_1);
+                acc[79] += (double)v8_19_0;
+                acc[80] += (double)v9_4_0;
+                acc[81] += (double)v9_5_0;
+                acc[82] += (double)v9_6_0;
+                acc[83] += (double)v9_7_0;
+                acc[84] += (double)v9_8_0;
+                acc[85] += (double)v9_9_0;
+                const VT v9_10_0 = QCx * v9_4_0 + WQx * v9_4_1 + (VT)2.0 * oo2e * (v9_1_0 - rho_e * v9_1_1);
+                acc[86] += (double)v9_10_0;
+                const VT v9_11_0 = QCx * v9_5_0 + WQx * v9_5_1 + (VT)1.0 * oo2e * (v9_2_0 - rho_e * v9_2_1);
+                acc[87] += (double)v9_11_0;
+                const VT v9_12_0 = QCx * v9_6_0 + WQx * v9_6_1 + (VT)1.0 * oo2e * (v9_3_0 - rho_e * v9_3_1);
+                acc[88] += (double)v9_12_0;
+                const VT v9_13_0 = QCy * v9_5_0 + WQy * v9_5_1 + (VT)1.0 * oo2e * (v9_1_0 - rho_e * v9_1_1);
+                acc[89] += (double)v9_13_0;
+                const VT v9_14_0 = QCz * v9_6_0 + WQz * v9_6_1 + (VT)2.0 * oo2ze * v3_6_1 + (VT)1.0 * oo2e * (v9_1_0 - rho_e * v9_1_1);
+                acc[90] += (double)v9_14_0;
+                const VT v9_15_0 = QCx * v9_8_0 + WQx * v9_8_1;
+                acc[91] += (double)v9_15_0;
+                const VT v9_16_0 = QCy * v9_7_0 + WQy * v9_7_1 + (VT)2.0 * oo2e * (v9_2_0 - rho_e * v9_2_1);
+                acc[92] += (double)v9_16_0;
+                const VT v9_17_0 = QCy * v9_8_0 + WQy * v9_8_1 + (VT)1.0 * oo2e * (v9_3_0 - rho_e * v9_3_1);
+                acc[93] += (double)v9_17_0;
+                const VT v9_18_0 = QCz * v9_8_0 + WQz * v9_8_1 + (VT)2.0 * oo2ze * v3_8_1 + (VT)1.0 * oo2e * (v9_2_0 - rho_e * v9_2_1);
+                acc[94] += (double)v9_18_0;
+                const VT v9_19_0 = QCz * v9_9_0 + WQz * v9_9_1 + (VT)2.0 * oo2ze * v3_9_1 + (VT)2.0 * oo2e * (v9_3_0 - rho_e * v9_3_1);
+                acc[95] += (double)v9_19_0;
+                acc[96] += (double)v10_4_0;
+                acc[97] += (double)v10_5_0;
+                acc[98] += (double)v10_6_0;
+                acc[99] += (double)v10_7_0;
+                acc[100] += (double)v10_8_0;
+                acc[101] += (double)v10_9_0;
+                const VT v10_10_0 = QCx * v10_4_0 + WQx * v10_4_1 + (VT)3.0 * oo2ze * v4_4_1 + (VT)2.0 * oo2e * (v10_1_0 - rho_e * v10_1_1);
+                acc[102] += (double)v10_10_0;
+                const VT v10_11_0 = QCx * v10_5_0 + WQx * v10_5_1 + (VT)3.0 * oo2ze * v4_5_1 + (VT)1.0 * oo2e * (v10_2_0 - rho_e * v10_2_1);
+                acc[103] += (double)v10_11_0;
+                const VT v10_12_0 = QCx * v10_6_0 + WQx * v10_6_1 + (VT)3.0 * oo2ze * v4_6_1 + (VT)1.0 * oo2e * (v10_3_0 - rho_e * v10_3_1);
+                acc[104] += (double)v10_12_0;
+                const VT v10_13_0 = QCy * v10_5_0 + WQy * v10_5_1 + (VT)1.0 * oo2e * (v10_1_0 - rho_e * v10_1_1);
+                acc[105] += (double)v10_13_0;
+                const VT v10_14_0 = QCz * v10_6_0 + WQz * v10_6_1 + (VT)1.0 * oo2e * (v10_1_0 - rho_e * v10_1_1);
+                acc[106] += (double)v10_14_0;
+                const VT v10_15_0 = QCx * v10_8_0 + WQx * v10_8_1 + (VT)3.0 * oo2ze * v4_8_1;
+                acc[107] += (double)v10_15_0;
+                const VT v10_16_0 = QCy * v10_7_0 + WQy * v10_7_1 + (VT)2.0 * oo2e * (v10_2_0 - rho_e * v10_2_1);
+                acc[108] += (double)v10_16_0;
+                const VT v10_17_0 = QCy * v10_8_0 + WQy * v10_8_1 + (VT)1.0 * oo2e * (v10_3_0 - rho_e * v10_3_1);
+                acc[109] += (double)v10_17_0;
+                const VT v10_18_0 = QCz * v10_8_0 + WQz * v10_8_1 + (VT)1.0 * oo2e * (v10_2_0 - rho_e * v10_2_1);
+                acc[110] += (double)v10_18_0;
+                const VT v10_19_0 = QCz * v10_9_0 + WQz * v10_9_1 + (VT)2.0 * oo2e * (v10_3_0 - rho_e * v10_3_1);
+                acc[111] += (double)v10_19_0;
+                acc[112] += (double)v11_4_0;
+                acc[113] += (double)v11_5_0;
+                acc[114] += (double)v11_6_0;
+                acc[115] += (double)v11_7_0;
+                acc[116] += (double)v11_8_0;
+                acc[117] += (double)v11_9_0;
+                const VT v11_10_0 = QCx * v11_4_0 + WQx * v11_4_1 + (VT)2.0 * oo2ze * v5_4_1 + (VT)2.0 * oo2e * (v11_1_0 - rho_e * v11_1_1);
+                acc[118] += (double)v11_10_0;
+                const VT v11_11_0 = QCx * v11_5_0 + WQx * v11_5_1 + (VT)2.0 * oo2ze * v5_5_1 + (VT)1.0 * oo2e * (v11_2_0 - rho_e * v11_2_1);
+                acc[119] += (double)v11_11_0;
+                const VT v11_12_0 = QCx * v11_6_0 + WQx * v11_6_1 + (VT)2.0 * oo2ze * v5_6_1 + (VT)1.0 * oo2e * (v11_3_0 - rho_e * v11_3_1);
+                acc[120] += (double)v11_12_0;
+                const VT v11_13_0 = QCy * v11_5_0 + WQy * v11_5_1 + (VT)1.0 * oo2ze * v4_5_1 + (VT)1.0 * oo2e * (v11_1_0 - rho_e * v11_1_1);
+                acc[121] += (double)v11_13_0;
+                const VT v11_14_0 = QCz * v11_6_0 + WQz * v11_6_1 + (VT)1.0 * oo2e * (v11_1_0 - rho_e * v11_1_1);
+                acc[122] += (double)v11_14_0;
+                const VT v11_15_0 = QCx * v11_8_0 + WQx * v11_8_1 + (VT)2.0 * oo2ze * v5_8_1;
+                acc[123] += (double)v11_15_0;
+                const VT v11_16_0 = QCy * v11_7_0 + WQy * v11_7_1 + (VT)1.0 * oo2ze * v4_7_1 + (VT)2.0 * oo2e * (v11_2_0 - rho_e * v11_2_1);
+                acc[124] += (double)v11_16_0;
+                const VT v11_17_0 = QCy * v11_8_0 + WQy * v11_8_1 + (VT)1.0 * oo2ze * v4_8_1 + (VT)1.0 * oo2e * (v11_3_0 - rho_e * v11_3_1);
+                acc[125] += (double)v11_17_0;
+                const VT v11_18_0 = QCz * v11_8_0 + WQz * v11_8_1 + (VT)1.0 * oo2e * (v11_2_0 - rho_e * v11_2_1);
+                acc[126] += (double)v11_18_0;
+                const VT v11_19_0 = QCz * v11_9_0 + WQz * v11_9_1 + (VT)2.0 * oo2e * (v11_3_0 - rho_e * v11_3_1);
+                acc[127] += (double)v11_19_0;
+                acc[128] += (double)v12_4_0;
+                acc[129] += (double)v12_5_0;
+                acc[130] += (double)v12_6_0;
+                acc[131] += (double)v12_7_0;
+                acc[132] += (double)v12_8_0;
+                acc[133] += (double)v12_9_0;
+                const VT v12_10_0 = QCx * v12_4_0 + WQx * v12_4_1 + (VT)2.0 * oo2ze * v6_4_1 + (VT)2.0 * oo2e * (v12_1_0 - rho_e * v12_1_1);
+                acc[134] += (double)v12_10_0;
+                const VT v12_11_0 = QCx * v12_5_0 + WQx * v12_5_1 + (VT)2.0 * oo2ze * v6_5_1 + (VT)1.0 * oo2e * (v12_2_0 - rho_e * v12_2_1);
+                acc[135] += (double)v12_11_0;
+                const VT v12_12_0 = QCx * v12_6_0 + WQx * v12_6_1 + (VT)2.0 * oo2ze * v6_6_1 + (VT)1.0 * oo2e * (v12_3_0 - rho_e * v12_3_1);
+                acc[136] += (double)v12_12_0;
+                const VT v12_13_0 = QCy * v12_5_0 + WQy * v12_5_1 + (VT)1.0 * oo2e * (v12_1_0 - rho_e * v12_1_1);
+                acc[137] += (double)v12_13_0;
+                const VT v12_14_0 = QCz * v12_6_0 + WQz * v12_6_1 + (VT)1.0 * oo2ze * v4_6_1 + (VT)1.0 * oo2e * (v12_1_0 - rho_e * v12_1_1);
+                acc[138] += (double)v12_14_0;
+                const VT v12_15_0 = QCx * v12_8_0 + WQx * v12_8_1 + (VT)2.0 * oo2ze * v6_8_1;
+                acc[139] += (double)v12_15_0;
+                const VT v12_16_0 = QCy * v12_7_0 + WQy * v12_7_1 + (VT)2.0 * oo2e * (v12_2_0 - rho_e * v12_2_1);
+                acc[140] += (double)v12_16_0;
+                const VT v12_17_0 = QCy * v12_8_0 + WQy * v12_8_1 + (VT)1.0 * oo2e * (v12_3_0 - rho_e * v12_3_1);
+                acc[141] += (double)v12_17_0;
+                const VT v12_18_0 = QCz * v12_8_0 + WQz * v12_8_1 + (VT)1.0 * oo2ze * v4_8_1 + (VT)1.0 * oo2e * (v12_2_0 - rho_e * v12_2_1);
+                acc[142] += (double)v12_18_0;
+                const VT v12_19_0 = QCz * v12_9_0 + WQz * v12_9_1 + (VT)1.0 * oo2ze * v4_9_1 + (VT)2.0 * oo2e * (v12_3_0 - rho_e * v12_3_1);
+                acc[143] += (double)v12_19_0;
+                acc[144] += (double)v13_4_0;
+                acc[145] += (double)v13_5_0;
+                acc[146] += (double)v13_6_0;
+                acc[147] += (double)v13_7_0;
+                acc[148] += (double)v13_8_0;
+                acc[149] += (double)v13_9_0;
+                const VT v13_10_0 = QCx * v13_4_0 + WQx * v13_4_1 + (VT)1.0 * oo2ze * v7_4_1 + (VT)2.0 * oo2e * (v13_1_0 - rho_e * v13_1_1);
+                acc[150] += (double)v13_10_0;
+                const VT v13_11_0 = QCx * v13_5_0 + WQx * v13_5_1 + (VT)1.0 * oo2ze * v7_5_1 + (VT)1.0 * oo2e * (v13_2_0 - rho_e * v13_2_1);
+                acc[151] += (double)v13_11_0;
+                const VT v13_12_0 = QCx * v13_6_0 + WQx * v13_6_1 + (VT)1.0 * oo2ze * v7_6_1 + (VT)1.0 * oo2e * (v13_3_0 - rho_e * v13_3_1);
+                acc[152] += (double)v13_12_0;
+                const VT v13_13_0 = QCy * v13_5_0 + WQy * v13_5_1 + (VT)2.0 * oo2ze * v5_5_1 + (VT)1.0 * oo2e * (v13_1_0 - rho_e * v13_1_1);
+                acc[153] += (double)v13_13_0;
+                const VT v13_14_0 = QCz * v13_6_0 + WQz * v13_6_1 + (VT)1.0 * oo2e * (v13_1_0 - rho_e * v13_1_1);
+                acc[154] += (double)v13_14_0;
+                const VT v13_15_0 = QCx * v13_8_0 + WQx * v13_8_1 + (VT)1.0 * oo2ze * v7_8_1;
+                acc[155] += (double)v13_15_0;
+                const VT v13_16_0 = QCy * v13_7_0 + WQy * v13_7_1 + (VT)2.0 * oo2ze * v5_7_1 + (VT)2.0 * oo2e * (v13_2_0 - rho_e * v13_2_1);
+                acc[156] += (double)v13_16_0;
+                const VT v13_17_0 = QCy * v13_8_0 + WQy * v13_8_1 + (VT)2.0 * oo2ze * v5_8_1 + (VT)1.0 * oo2e * (v13_3_0 - rho_e * v13_3_1);
+                acc[157] += (double)v13_17_0;
+                const VT v13_18_0 = QCz * v13_8_0 + WQz * v13_8_1 + (VT)1.0 * oo2e * (v13_2_0 - rho_e * v13_2_1);
+                acc[158] += (double)v13_18_0;
+                const VT v13_19_0 = QCz * v13_9_0 + WQz * v13_9_1 + (VT)2.0 * oo2e * (v13_3_0 - rho_e * v13_3_1);
+                acc[159] += (double)v13_19_0;
+                acc[160] += (double)v14_4_0;
+                acc[161] += (double)v14_5_0;
+                acc[162] += (double)v14_6_0;
+                acc[163] += (double)v14_7_0;
+                acc[164] += (double)v14_8_0;
+                acc[165] += (double)v14_9_0;
+                const VT v14_10_0 = QCx * v14_4_0 + WQx * v14_4_1 + (VT)1.0 * oo2ze * v9_4_1 + (VT)2.0 * oo2e * (v14_1_0 - rho_e * v14_1_1);
+                acc[166] += (double)v14_10_0;
+                const VT v14_11_0 = QCx * v14_5_0 + WQx * v14_5_1 + (VT)1.0 * oo2ze * v9_5_1 + (VT)1.0 * oo2e * (v14_2_0 - rho_e * v14_2_1);
+                acc[167] += (double)v14_11_0;
+                const VT v14_12_0 = QCx * v14_6_0 + WQx * v14_6_1 + (VT)1.0 * oo2ze * v9_6_1 + (VT)1.0 * oo2e * (v14_3_0 - rho_e * v14_3_1);
+                acc[168] += (double)v14_12_0;
+                const VT v14_13_0 = QCy * v14_5_0 + WQy * v14_5_1 + (VT)1.0 * oo2e * (v14_1_0 - rho_e * v14_1_1);
+                acc[169] += (double)v14_13_0;
+                const VT v14_14_0 = QCz * v14_6_0 + WQz * v14_6_1 + (VT)2.0 * oo2ze * v6_6_1 + (VT)1.0 * oo2e * (v14_1_0 - rho_e * v14_1_1);
+                acc[170] += (double)v14_14_0;
+                const VT v14_15_0 = QCx * v14_8_0 + WQx * v14_8_1 + (VT)1.0 * oo2ze * v9_8_1;
+                acc[171] += (double)v14_15_0;
+                const VT v14_16_0 = QCy * v14_7_0 + WQy * v14_7_1 + (VT)2.0 * oo2e * (v14_2_0 - rho_e * v14_2_1);
+                acc[172] += (double)v14_16_0;
+                const VT v14_17_0 = QCy * v14_8_0 + WQy * v14_8_1 + (VT)1.0 * oo2e * (v14_3_0 - rho_e * v14_3_1);
+                acc[173] += (double)v14_17_0;
+                const VT v14_18_0 = QCz * v14_8_0 + WQz * v14_8_1 + (VT)2.0 * oo2ze * v6_8_1 + (VT)1.0 * oo2e * (v14_2_0 - rho_e * v14_2_1);
+                acc[174] += (double)v14_18_0;
+                const VT v14_19_0 = QCz * v14_9_0 + WQz * v14_9_1 + (VT)2.0 * oo2ze * v6_9_1 + (VT)2.0 * oo2e * (v14_3_0 - rho_e * v14_3_1);
+                acc[175] += (double)v14_19_0;
+                acc[176] += (double)v15_4_0;
+                acc[177] += (double)v15_5_0;
+                acc[178] += (double)v15_6_0;
+                acc[179] += (double)v15_7_0;
+                acc[180] += (double)v15_8_0;
+                acc[181] += (double)v15_9_0;
+                const VT v15_10_0 = QCx * v15_4_0 + WQx * v15_4_1 + (VT)1.0 * oo2ze * v8_4_1 + (VT)2.0 * oo2e * (v15_1_0 - rho_e * v15_1_1);
+                acc[182] += (double)v15_10_0;
+                const VT v15_11_0 = QCx * v15_5_0 + WQx * v15_5_1 + (VT)1.0 * oo2ze * v8_5_1 + (VT)1.0 * oo2e * (v15_2_0 - rho_e * v15_2_1);
+                acc[183] += (double)v15_11_0;
+                const VT v15_12_0 = QCx * v15_6_0 + WQx * v15_6_1 + (VT)1.0 * oo2ze * v8_6_1 + (VT)1.0 * oo2e * (v15_3_0 - rho_e * v15_3_1);
+                acc[184] += (double)v15_12_0;
+                const VT v15_13_0 = QCy * v15_5_0 + WQy * v15_5_1 + (VT)1.0 * oo2ze * v6_5_1 + (VT)1.0 * oo2e * (v15_1_0 - rho_e * v15_1_1);
+                acc[185] += (double)v15_13_0;
+                const VT v15_14_0 = QCz * v15_6_0 + WQz * v15_6_1 + (VT)1.0 * oo2ze * v5_6_1 + (VT)1.0 * oo2e * (v15_1_0 - rho_e * v15_1_1);
+                acc[186] += (double)v15_14_0;
+                const VT v15_15_0 = QCx * v15_8_0 + WQx * v15_8_1 + (VT)1.0 * oo2ze * v8_8_1;
+                acc[187] += (double)v15_15_0;
+                const VT v15_16_0 = QCy * v15_7_0 + WQy * v15_7_1 + (VT)1.0 * oo2ze * v6_7_1 + (VT)2.0 * oo2e * (v15_2_0 - rho_e * v15_2_1);
+                acc[188] += (double)v15_16_0;
+                const VT v15_17_0 = QCy * v15_8_0 + WQy * v15_8_1 + (VT)1.0 * oo2ze * v6_8_1 + (VT)1.0 * oo2e * (v15_3_0 - rho_e * v15_3_1);
+                acc[189] += (double)v15_17_0;
+                const VT v15_18_0 = QCz * v15_8_0 + WQz * v15_8_1 + (VT)1.0 * oo2ze * v5_8_1 + (VT)1.0 * oo2e * (v15_2_0 - rho_e * v15_2_1);
+                acc[190] += (double)v15_18_0;
+                const VT v15_19_0 = QCz * v15_9_0 + WQz * v15_9_1 + (VT)1.0 * oo2ze * v5_9_1 + (VT)2.0 * oo2e * (v15_3_0 - rho_e * v15_3_1);
+                acc[191] += (double)v15_19_0;
+                acc[192] += (double)v16_4_0;
+                acc[193] += (double)v16_5_0;
+                acc[194] += (double)v16_6_0;
+                acc[195] += (double)v16_7_0;
+                acc[196] += (double)v16_8_0;
+                acc[197] += (double)v16_9_0;
+                const VT v16_10_0 = QCx * v16_4_0 + WQx * v16_4_1 + (VT)2.0 * oo2e * (v16_1_0 - rho_e * v16_1_1);
+                acc[198] += (double)v16_10_0;
+                const VT v16_11_0 = QCx * v16_5_0 + WQx * v16_5_1 + (VT)1.0 * oo2e * (v16_2_0 - rho_e * v16_2_1);
+                acc[199] += (double)v16_11_0;
+                const VT v16_12_0 = QCx * v16_6_0 + WQx * v16_6_1 + (VT)1.0 * oo2e * (v16_3_0 - rho_e * v16_3_1);
+                acc[200] += (double)v16_12_0;
+                const VT v16_13_0 = QCy * v16_5_0 + WQy * v16_5_1 + (VT)3.0 * oo2ze * v7_5_1 + (VT)1.0 * oo2e * (v16_1_0 - rho_e * v16_1_1);
+                acc[201] += (double)v16_13_0;
+                const VT v16_14_0 = QCz * v16_6_0 + WQz * v16_6_1 + (VT)1.0 * oo2e * (v16_1_0 - rho_e * v16_1_1);
+                acc[202] += (double)v16_14_0;
+                const VT v16_15_0 = QCx * v16_8_0 + WQx * v16_8_1;
+                acc[203] += (double)v16_15_0;
+                const VT v16_16_0 = QCy * v16_7_0 + WQy * v16_7_1 + (VT)3.0 * oo2ze * v7_7_1 + (VT)2.0 * oo2e * (v16_2_0 - rho_e * v16_2_1);
+                acc[204] += (double)v16_16_0;
+                const VT v16_17_0 = QCy * v16_8_0 + WQy * v16_8_1 + (VT)3.0 * oo2ze * v7_8_1 + (VT)1.0 * oo2e * (v16_3_0 - rho_e * v16_3_1);
+                acc[205] += (double)v16_17_0;
+                const VT v16_18_0 = QCz * v16_8_0 + WQz * v16_8_1 + (VT)1.0 * oo2e * (v16_2_0 - rho_e * v16_2_1);
+                acc[206] += (double)v16_18_0;
+                const VT v16_19_0 = QCz * v16_9_0 + WQz * v16_9_1 + (VT)2.0 * oo2e * (v16_3_0 - rho_e * v16_3_1);
+                acc[207] += (double)v16_19_0;
+                acc[208] += (double)v17_4_0;
+                acc[209] += (double)v17_5_0;
+                acc[210] += (double)v17_6_0;
+                acc[211] += (double)v17_7_0;
+                acc[212] += (double)v17_8_0;
+                acc[213] += (double)v17_9_0;
+                const VT v17_10_0 = QCx * v17_4_0 + WQx * v17_4_1 + (VT)2.0 * oo2e * (v17_1_0 - rho_e * v17_1_1);
+                acc[214] += (double)v17_10_0;
+                const VT v17_11_0 = QCx * v17_5_0 + WQx * v17_5_1 + (VT)1.0 * oo2e * (v17_2_0 - rho_e * v17_2_1);
+                acc[215] += (double)v17_11_0;
+                const VT v17_12_0 = QCx * v17_6_0 + WQx * v17_6_1 + (VT)1.0 * oo2e * (v17_3_0 - rho_e * v17_3_1);
+                acc[216] += (double)v17_12_0;
+                const VT v17_13_0 = QCy * v17_5_0 + WQy * v17_5_1 + (VT)2.0 * oo2ze * v8_5_1 + (VT)1.0 * oo2e * (v17_1_0 - rho_e * v17_1_1);
+                acc[217] += (double)v17_13_0;
+                const VT v17_14_0 = QCz * v17_6_0 + WQz * v17_6_1 + (VT)1.0 * oo2ze * v7_6_1 + (VT)1.0 * oo2e * (v17_1_0 - rho_e * v17_1_1);
+                acc[218] += (double)v17_14_0;
+                const VT v17_15_0 = QCx * v17_8_0 + WQx * v17_8_1;
+                acc[219] += (double)v17_15_0;
+                const VT v17_16_0 = QCy * v17_7_0 + WQy * v17_7_1 + (VT)2.0 * oo2ze * v8_7_1 + (VT)2.0 * oo2e * (v17_2_0 - rho_e * v17_2_1);
+                acc[220] += (double)v17_16_0;
+                const VT v17_17_0 = QCy * v17_8_0 + WQy * v17_8_1 + (VT)2.0 * oo2ze * v8_8_1 + (VT)1.0 * oo2e * (v17_3_0 - rho_e * v17_3_1);
+                acc[221] += (double)v17_17_0;
+                const VT v17_18_0 = QCz * v17_8_0 + WQz * v17_8_1 + (VT)1.0 * oo2ze * v7_8_1 + (VT)1.0 * oo2e * (v17_2_0 - rho_e * v17_2_1);
+                acc[222] += (double)v17_18_0;
+                const VT v17_19_0 = QCz * v17_9_0 + WQz * v17_9_1 + (VT)1.0 * oo2ze * v7_9_1 + (VT)2.0 * oo2e * (v17_3_0 - rho_e * v17_3_1);
+                acc[223] += (double)v17_19_0;
+                acc[224] += (double)v18_4_0;
+                acc[225] += (double)v18_5_0;
+                acc[226] += (double)v18_6_0;
+                acc[227] += (double)v18_7_0;
+                acc[228] += (double)v18_8_0;
+                acc[229] += (double)v18_9_0;
+                const VT v18_10_0 = QCx * v18_4_0 + WQx * v18_4_1 + (VT)2.0 * oo2e * (v18_1_0 - rho_e * v18_1_1);
+                acc[230] += (double)v18_10_0;
+                const VT v18_11_0 = QCx * v18_5_0 + WQx * v18_5_1 + (VT)1.0 * oo2e * (v18_2_0 - rho_e * v18_2_1);
+                acc[231] += (double)v18_11_0;
+                const VT v18_12_0 = QCx * v18_6_0 + WQx * v18_6_1 + (VT)1.0 * oo2e * (v18_3_0 - rho_e * v18_3_1);
+                acc[232] += (double)v18_12_0;
+                const VT v18_13_0 = QCy * v18_5_0 + WQy * v18_5_1 + (VT)1.0 * oo2ze * v9_5_1 + (VT)1.0 * oo2e * (v18_1_0 - rho_e * v18_1_1);
+                acc[233] += (double)v18_13_0;
+                const VT v18_14_0 = QCz * v18_6_0 + WQz * v18_6_1 + (VT)2.0 * oo2ze * v8_6_1 + (VT)1.0 * oo2e * (v18_1_0 - rho_e * v18_1_1);
+                acc[234] += (double)v18_14_0;
+                const VT v18_15_0 = QCx * v18_8_0 + WQx * v18_8_1;
+                acc[235] += (double)v18_15_0;
+                const VT v18_16_0 = QCy * v18_7_0 + WQy * v18_7_1 + (VT)1.0 * oo2ze * v9_7_1 + (VT)2.0 * oo2e * (v18_2_0 - rho_e * v18_2_1);
+                acc[236] += (double)v18_16_0;
+                const VT v18_17_0 = QCy * v18_8_0 + WQy * v18_8_1 + (VT)1.0 * oo2ze * v9_8_1 + (VT)1.0 * oo2e * (v18_3_0 - rho_e * v18_3_1);
+                acc[237] += (double)v18_17_0;
+                const VT v18_18_0 = QCz * v18_8_0 + WQz * v18_8_1 + (VT)2.0 * oo2ze * v8_8_1 + (VT)1.0 * oo2e * (v18_2_0 - rho_e * v18_2_1);
+                acc[238] += (double)v18_18_0;
+                const VT v18_19_0 = QCz * v18_9_0 + WQz * v18_9_1 + (VT)2.0 * oo2ze * v8_9_1 + (VT)2.0 * oo2e * (v18_3_0 - rho_e * v18_3_1);
+                acc[239] += (double)v18_19_0;
+                acc[240] += (double)v19_4_0;
+                acc[241] += (double)v19_5_0;
+                acc[242] += (double)v19_6_0;
+                acc[243] += (double)v19_7_0;
+                acc[244] += (double)v19_8_0;
+                acc[245] += (double)v19_9_0;
+                const VT v19_10_0 = QCx * v19_4_0 + WQx * v19_4_1 + (VT)2.0 * oo2e * (v19_1_0 - rho_e * v19_1_1);
+                acc[246] += (double)v19_10_0;
+                const VT v19_11_0 = QCx * v19_5_0 + WQx * v19_5_1 + (VT)1.0 * oo2e * (v19_2_0 - rho_e * v19_2_1);
+                acc[247] += (double)v19_11_0;
+                const VT v19_12_0 = QCx * v19_6_0 + WQx * v19_6_1 + (VT)1.0 * oo2e * (v19_3_0 - rho_e * v19_3_1);
+                acc[248] += (double)v19_12_0;
+                const VT v19_13_0 = QCy * v19_5_0 + WQy * v19_5_1 + (VT)1.0 * oo2e * (v19_1_0 - rho_e * v19_1_1);
+                acc[249] += (double)v19_13_0;
+                const VT v19_14_0 = QCz * v19_6_0 + WQz * v19_6_1 + (VT)3.0 * oo2ze * v9_6_1 + (VT)1.0 * oo2e * (v19_1_0 - rho_e * v19_1_1);
+                acc[250] += (double)v19_14_0;
+                const VT v19_15_0 = QCx * v19_8_0 + WQx * v19_8_1;
+                acc[251] += (double)v19_15_0;
+                const VT v19_16_0 = QCy * v19_7_0 + WQy * v19_7_1 + (VT)2.0 * oo2e * (v19_2_0 - rho_e * v19_2_1);
+                acc[252] += (double)v19_16_0;
+                const VT v19_17_0 = QCy * v19_8_0 + WQy * v19_8_1 + (VT)1.0 * oo2e * (v19_3_0 - rho_e * v19_3_1);
+                acc[253] += (double)v19_17_0;
+                const VT v19_18_0 = QCz * v19_8_0 + WQz * v19_8_1 + (VT)3.0 * oo2ze * v9_8_1 + (VT)1.0 * oo2e * (v19_2_0 - rho_e * v19_2_1);
+                acc[254] += (double)v19_18_0;
+                const VT v19_19_0 = QCz * v19_9_0 + WQz * v19_9_1 + (VT)3.0 * oo2ze * v9_9_1 + (VT)2.0 * oo2e * (v19_3_0 - rho_e * v19_3_1);
+                acc[255] += (double)v19_19_0;
+            }
         }
     }
 }

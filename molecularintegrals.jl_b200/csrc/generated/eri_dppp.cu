@@ -25,13 +25,13 @@ __device__ __forceinline__ void vrr_dppp(const PairTab &P, const BoysTab &B, int
             const double r = rsqrt(bra.zeta + ket.zeta);
             const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
-            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[6];
             boys_fm<5>(T, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
-            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
             const VT WQx = (VT)(zz * PQx), WQy = (VT)(zz * PQy), WQz = (VT)(zz * PQz);
             const VT oo2z = (VT)bra.oo2z, oo2e = (VT)ket.oo2z, oo2ze = (VT)(0.5 * r2);
@@ -219,246 +219,393 @@ __device__ __forceinline__ void vrr_dppp(const PairTab &P, const BoysTab &B, int
             const VT v18_3_1 = QCz * v18_0_1 + WQz * v18_0_2 + (VT)2.0 * oo2ze * v8_0_2;
             const VT v19_3_0 = QCz * v19_0_0 + WQz * v19_0_1 + (VT)3.0 * oo2ze * v9_0_1;
             const VT v19_3_1 = QCz * v19_0_1 + WQz * v19_0_2 + (VT)3.0 * oo2ze * v9_0_2;
-            const VT v4_4_0 = QCx * v4_1_0 + WQx * v4_1_1 + (VT)2.0 * oo2ze * v1_1_1 + (VT)1.0 * oo2e * (v4_0_0 - rho_e * v4_0_1);
-            const VT v5_4_0 = QCx * v5_1_0 + WQx * v5_1_1 + (VT)1.0 * oo2ze * v2_1_1 + (VT)1.0 * oo2e * (v5_0_0 - rho_e * v5_0_1);
-            const VT v6_4_0 = QCx * v6_1_0 + WQx * v6_1_1 + (VT)1.0 * oo2ze * v3_1_1 + (VT)1.0 * oo2e * (v6_0_0 - rho_e * v6_0_1);
-            const VT v7_4_0 = QCx * v7_1_0 + WQx * v7_1_1 + (VT)1.0 * oo2e * (v7_0_0 - rho_e * v7_0_1);
-            const VT v8_4_0 = QCx * v8_1_0 + WQx * v8_1_1 + (VT)1.0 * oo2e * (v8_0_0 - rho_e * v8_0_1);
-            const VT v9_4_0 = QCx * v9_1_0 + WQx * v9_1_1 + (VT)1.0 * oo2e * (v9_0_0 - rho_e * v9_0_1);
-            const VT v10_4_0 = QCx * v10_1_0 + WQx * v10_1_1 + (VT)3.0 * oo2ze * v4_1_1 + (VT)1.0 * oo2e * (v10_0_0 - rho_e * v10_0_1);
-            const VT v11_4_0 = QCx * v11_1_0 + WQx * v11_1_1 + (VT)2.0 * oo2ze * v5_1_1 + (VT)1.0 * oo2e * (v11_0_0 - rho_e * v11_0_1);
-            const VT v12_4_0 = QCx * v12_1_0 + WQx * v12_1_1 + (VT)2.0 * oo2ze * v6_1_1 + (VT)1.0 * oo2e * (v12_0_0 - rho_e * v12_0_1);
-            const VT v13_4_0 = QCx * v13_1_0 + WQx * v13_1_1 + (VT)1.0 * oo2ze * v7_1_1 + (VT)1.0 * oo2e * (v13_0_0 - rho_e * v13_0_1);
-            const VT v14_4_0 = QCx * v14_1_0 + WQx * v14_1_1 + (VT)1.0 * oo2ze * v9_1_1 + (VT)1.0 * oo2e * (v14_0_0 - rho_e * v14_0_1);
-            const VT v15_4_0 = QCx * v15_1_0 + WQx * v15_1_1 + (VT)1.0 * oo2ze * v8_1_1 + (VT)1.0 * oo2e * (v15_0_0 - rho_e * v15_0_1);
-            const VT v16_4_0 = QCx * v16_1_0 + WQx * v16_1_1 + (VT)1.0 * oo2e * (v16_0_0 - rho_e * v16_0_1);
-            const VT v17_4_0 = QCx * v17_1_0 + WQx * v17_1_1 + (VT)1.0 * oo2e * (v17_0_0 - rho_e * v17_0_1);
-            const VT v18_4_0 = QCx * v18_1_0 + WQx * v18_1_1 + (VT)1.0 * oo2e * (v18_0_0 - rho_e * v18_0_1);
-            const VT v19_4_0 = QCx * v19_1_0 + WQx * v19_1_1 + (VT)1.0 * oo2e * (v19_0_0 - rho_e * v19_0_1);
-            const VT v4_5_0 = QCx * v4_2_0 + WQx * v4_2_1 + (VT)2.0 * oo2ze * v1_2_1;
-            const VT v5_5_0 = QCx * v5_2_0 + WQx * v5_2_1 + (VT)1.0 * oo2ze * v2_2_1;
-            const VT v6_5_0 = QCx * v6_2_0 + WQx * v6_2_1 + (VT)1.0 * oo2ze * v3_2_1;
-            const VT v7_5_0 = QCx * v7_2_0 + WQx * v7_2_1;
-            const VT v8_5_0 = QCx * v8_2_0 + WQx * v8_2_1;
-            const VT v9_5_0 = QCx * v9_2_0 + WQx * v9_2_1;
-            const VT v10_5_0 = QCx * v10_2_0 + WQx * v10_2_1 + (VT)3.0 * oo2ze * v4_2_1;
-            const VT v11_5_0 = QCx * v11_2_0 + WQx * v11_2_1 + (VT)2.0 * oo2ze * v5_2_1;
-            const VT v12_5_0 = QCx * v12_2_0 + WQx * v12_2_1 + (VT)2.0 * oo2ze * v6_2_1;
-            const VT v13_5_0 = QCx * v13_2_0 + WQx * v13_2_1 + (VT)1.0 * oo2ze * v7_2_1;
-            const VT v14_5_0 = QCx * v14_2_0 + WQx * v14_2_1 + (VT)1.0 * oo2ze * v9_2_1;
-            const VT v15_5_0 = QCx * v15_2_0 + WQx * v15_2_1 + (VT)1.0 * oo2ze * v8_2_1;
-            const VT v16_5_0 = QCx * v16_2_0 + WQx * v16_2_1;
-            const VT v17_5_0 = QCx * v17_2_0 + WQx * v17_2_1;
-            const VT v18_5_0 = QCx * v18_2_0 + WQx * v18_2_1;
-            const VT v19_5_0 = QCx * v19_2_0 + WQx * v19_2_1;
-            const VT v4_6_0 = QCx * v4_3_0 + WQx * v4_3_1 + (VT)2.0 * oo2ze * v1_3_1;
-            const VT v5_6_0 = QCx * v5_3_0 + WQx * v5_3_1 + (VT)1.0 * oo2ze * v2_3_1;
-            const VT v6_6_0 = QCx * v6_3_0 + WQx * v6_3_1 + (VT)1.0 * oo2ze * v3_3_1;
-            const VT v7_6_0 = QCx * v7_3_0 + WQx * v7_3_1;
-            const VT v8_6_0 = QCx * v8_3_0 + WQx * v8_3_1;
-            const VT v9_6_0 = QCx * v9_3_0 + WQx * v9_3_1;
-            const VT v10_6_0 = QCx * v10_3_0 + WQx * v10_3_1 + (VT)3.0 * oo2ze * v4_3_1;
-            const VT v11_6_0 = QCx * v11_3_0 + WQx * v11_3_1 + (VT)2.0 * oo2ze * v5_3_1;
-            const VT v12_6_0 = QCx * v12_3_0 + WQx * v12_3_1 + (VT)2.0 * oo2ze * v6_3_1;
-            const VT v13_6_0 = QCx * v13_3_0 + WQx * v13_3_1 + (VT)1.0 * oo2ze * v7_3_1;
-            const VT v14_6_0 = QCx * v14_3_0 + WQx * v14_3_1 + (VT)1.0 * oo2ze * v9_3_1;
-            const VT v15_6_0 = QCx * v15_3_0 + WQx * v15_3_1 + (VT)1.0 * oo2ze * v8_3_1;
-            const VT v16_6_0 = QCx * v16_3_0 + WQx * v16_3_1;
-            const VT v17_6_0 = QCx * v17_3_0 + WQx * v17_3_1;
-            const VT v18_6_0 = QCx * v18_3_0 + WQx * v18_3_1;
-            const VT v19_6_0 = QCx * v19_3_0 + WQx * v19_3_1;
-            const VT v4_7_0 = QCy * v4_2_0 + WQy * v4_2_1 + (VT)1.0 * oo2e * (v4_0_0 - rho_e * v4_0_1);
-            const VT v5_7_0 = QCy * v5_2_0 + WQy * v5_2_1 + (VT)1.0 * oo2ze * v1_2_1 + (VT)1.0 * oo2e * (v5_0_0 - rho_e * v5_0_1);
-            const VT v6_7_0 = QCy * v6_2_0 + WQy * v6_2_1 + (VT)1.0 * oo2e * (v6_0_0 - rho_e * v6_0_1);
-            const VT v7_7_0 = QCy * v7_2_0 + WQy * v7_2_1 + (VT)2.0 * oo2ze * v2_2_1 + (VT)1.0 * oo2e * (v7_0_0 - rho_e * v7_0_1);
-            const VT v8_7_0 = QCy * v8_2_0 + WQy * v8_2_1 + (VT)1.0 * oo2ze * v3_2_1 + (VT)1.0 * oo2e * (v8_0_0 - rho_e * v8_0_1);
-            const VT v9_7_0 = QCy * v9_2_0 + WQy * v9_2_1 + (VT)1.0 * oo2e * (v9_0_0 - rho_e * v9_0_1);
-            const VT v10_7_0 = QCy * v10_2_0 + WQy * v10_2_1 + (VT)1.0 * oo2e * (v10_0_0 - rho_e * v10_0_1);
-            const VT v11_7_0 = QCy * v11_2_0 + WQy * v11_2_1 + (VT)1.0 * oo2ze * v4_2_1 + (VT)1.0 * oo2e * (v11_0_0 - rho_e * v11_0_1);
-            const VT v12_7_0 = QCy * v12_2_0 + WQy * v12_2_1 + (VT)1.0 * oo2e * (v12_0_0 - rho_e * v12_0_1);
-            const VT v13_7_0 = QCy * v13_2_0 + WQy * v13_2_1 + (VT)2.0 * oo2ze * v5_2_1 + (VT)1.0 * oo2e * (v13_0_0 - rho_e * v13_0_1);
-            const VT v14_7_0 = QCy * v14_2_0 + WQy * v14_2_1 + (VT)1.0 * oo2e * (v14_0_0 - rho_e * v14_0_1);
-            const VT v15_7_0 = QCy * v15_2_0 + WQy * v15_2_1 + (VT)1.0 * oo2ze * v6_2_1 + (VT)1.0 * oo2e * (v15_0_0 - rho_e * v15_0_1);
-            const VT v16_7_0 = QCy * v16_2_0 + WQy * v16_2_1 + (VT)3.0 * oo2ze * v7_2_1 + (VT)1.0 * oo2e * (v16_0_0 - rho_e * v16_0_1);
-            const VT v17_7_0 = QCy * v17_2_0 + WQy * v17_2_1 + (VT)2.0 * oo2ze * v8_2_1 + (VT)1.0 * oo2e * (v17_0_0 - rho_e * v17_0_1);
-            const VT v18_7_0 = QCy * v18_2_0 + WQy * v18_2_1 + (VT)1.0 * oo2ze * v9_2_1 + (VT)1.0 * oo2e * (v18_0_0 - rho_e * v18_0_1);
-            const VT v19_7_0 = QCy * v19_2_0 + WQy * v19_2_1 + (VT)1.0 * oo2e * (v19_0_0 - rho_e * v19_0_1);
-            const VT v4_8_0 = QCy * v4_3_0 + WQy * v4_3_1;
-            const VT v5_8_0 = QCy * v5_3_0 + WQy * v5_3_1 + (VT)1.0 * oo2ze * v1_3_1;
-            const VT v6_8_0 = QCy * v6_3_0 + WQy * v6_3_1;
-            const VT v7_8_0 = QCy * v7_3_0 + WQy * v7_3_1 + (VT)2.0 * oo2ze * v2_3_1;
-            const VT v8_8_0 = QCy * v8_3_0 + WQy * v8_3_1 + (VT)1.0 * oo2ze * v3_3_1;
-            const VT v9_8_0 = QCy * v9_3_0 + WQy * v9_3_1;
-            const VT v10_8_0 = QCy * v10_3_0 + WQy * v10_3_1;
-            const VT v11_8_0 = QCy * v11_3_0 + WQy * v11_3_1 + (VT)1.0 * oo2ze * v4_3_1;
-            const VT v12_8_0 = QCy * v12_3_0 + WQy * v12_3_1;
-            const VT v13_8_0 = QCy * v13_3_0 + WQy * v13_3_1 + (VT)2.0 * oo2ze * v5_3_1;
-            const VT v14_8_0 = QCy * v14_3_0 + WQy * v14_3_1;
-            const VT v15_8_0 = QCy * v15_3_0 + WQy * v15_3_1 + (VT)1.0 * oo2ze * v6_3_1;
-            const VT v16_8_0 = QCy * v16_3_0 + WQy * v16_3_1 + (VT)3.0 * oo2ze * v7_3_1;
-            const VT v17_8_0 = QCy * v17_3_0 + WQy * v17_3_1 + (VT)2.0 * oo2ze * v8_3_1;
-            const VT v18_8_0 = QCy * v18_3_0 + WQy * v18_3_1 + (VT)1.0 * oo2ze * v9_3_1;
-            const VT v19_8_0 = QCy * v19_3_0 + WQy * v19_3_1;
-            const VT v4_9_0 = QCz * v4_3_0 + WQz * v4_3_1 + (VT)1.0 * oo2e * (v4_0_0 - rho_e * v4_0_1);
-            const VT v5_9_0 = QCz * v5_3_0 + WQz * v5_3_1 + (VT)1.0 * oo2e * (v5_0_0 - rho_e * v5_0_1);
-            const VT v6_9_0 = QCz * v6_3_0 + WQz * v6_3_1 + (VT)1.0 * oo2ze * v1_3_1 + (VT)1.0 * oo2e * (v6_0_0 - rho_e * v6_0_1);
-            const VT v7_9_0 = QCz * v7_3_0 + WQz * v7_3_1 + (VT)1.0 * oo2e * (v7_0_0 - rho_e * v7_0_1);
-            const VT v8_9_0 = QCz * v8_3_0 + WQz * v8_3_1 + (VT)1.0 * oo2ze * v2_3_1 + (VT)1.0 * oo2e * (v8_0_0 - rho_e * v8_0_1);
-            const VT v9_9_0 = QCz * v9_3_0 + WQz * v9_3_1 + (VT)2.0 * oo2ze * v3_3_1 + (VT)1.0 * oo2e * (v9_0_0 - rho_e * v9_0_1);
-            const VT v10_9_0 = QCz * v10_3_0 + WQz * v10_3_1 + (VT)1.0 * oo2e * (v10_0_0 - rho_e * v10_0_1);
-            const VT v11_9_0 = QCz * v11_3_0 + WQz * v11_3_1 + (VT)1.0 * oo2e * (v11_0_0 - rho_e * v11_0_1);
-            const VT v12_9_0 = QCz * v12_3_0 + WQz * v12_3_1 + (VT)1.0 * oo2ze * v4_3_1 + (VT)1.0 * oo2e * (v12_0_0 - rho_e * v12_0_1);
-            const VT v13_9_0 = QCz * v13_3_0 + WQz * v13_3_1 + (VT)1.0 * oo2e * (v13_0_0 - rho_e * v13_0_1);
-            const VT v14_9_0 = QCz * v14_3_0 + WQz * v14_3_1 + (VT)2.0 * oo2ze * v6_3_1 + (VT)1.0 * oo2e * (v14_0_0 - rho_e * v14_0_1);
-            const VT v15_9_0 = QCz * v15_3_0 + WQz * v15_3_1 + (VT)1.0 * oo2ze * v5_3_1 + (VT)1.0 * oo2e * (v15_0_0 - rho_e * v15_0_1);
-            const VT v16_9_0 = QCz * v16_3_0 + WQz * v16_3_1 + (VT)1.0 * oo2e * (v16_0_0 - rho_e * v16_0_1);
-            const VT v17_9_0 = QCz * v17_3_0 + WQz * v17_3_1 + (VT)1.0 * oo2ze * v7_3_1 + (VT)1.0 * oo2e * (v17_0_0 - rho_e * v17_0_1);
-            const VT v18_9_0 = QCz * v18_3_0 + WQz * v18_3_1 + (VT)2.0 * oo2ze * v8_3_1 + (VT)1.0 * oo2e * (v18_0_0 - rho_e * v18_0_1);
-            const VT v19_9_0 = QCz * v19_3_0 + WQz * v19_3_1 + (VT)3.0 * oo2ze * v9_3_1 + (VT)1.0 * oo2e * (v19_0_0 - rho_e * v19_0_1);
-            acc[0] += (double)v4_1_0;
-            acc[1] += (double)v4_2_0;
-            acc[2] += (double)v4_3_0;
-            acc[3] += (double)v4_4_0;
-            acc[4] += (double)v4_5_0;
-            acc[5] += (double)v4_6_0;
-            acc[6] += (double)v4_7_0;
-            acc[7] += (double)v4_8_0;
-            acc[8] += (double)v4_9_0;
-            acc[9] += (double)v5_1_0;
-            acc[10] += (double)v5_2_0;
-            acc[11] += (double)v5_3_0;
-            acc[12] += (double)v5_4_0;
-            acc[13] += (double)v5_5_0;
-            acc[14] += (double)v5_6_0;
-            acc[15] += (double)v5_7_0;
-            acc[16] += (double)v5_8_0;
-            acc[17] += (double)v5_9_0;
-            acc[18] += (double)v6_1_0;
-            acc[19] += (double)v6_2_0;
-            acc[20] += (double)v6_3_0;
-            acc[21] += (double)v6_4_0;
-            acc[22] += (double)v6_5_0;
-            acc[23] += (double)v6_6_0;
-            acc[24] += (double)v6_7_0;
-            acc[25] += (double)v6_8_0;
-            acc[26] += (double)v6_9_0;
-            acc[27] += (double)v7_1_0;
-            acc[28] += (double)v7_2_0;
-            acc[29] += (double)v7_3_0;
-            acc[30] += (double)v7_4_0;
-            acc[31] += (double)v7_5_0;
-            acc[32] += (double)v7_6_0;
-            acc[33] += (double)v7_7_0;
-            acc[34] += (double)v7_8_0;
-            acc[35] += (double)v7_9_0;
-            acc[36] += (double)v8_1_0;
-            acc[37] += (double)v8_2_0;
-            acc[38] += (double)v8_3_0;
-            acc[39] += (double)v8_4_0;
-            acc[40] += (double)v8_5_0;
-            acc[41] += (double)v8_6_0;
-            acc[42] += (double)v8_7_0;
-            acc[43] += (double)v8_8_0;
-            acc[44] += (double)v8_9_0;
-            acc[45] += (double)v9_1_0;
-            acc[46] += (double)v9_2_0;
-            acc[47] += (double)v9_3_0;
-            acc[48] += (double)v9_4_0;
-            acc[49] += (double)v9_5_0;
-            acc[50] += (double)v9_6_0;
-            acc[51] += (double)v9_7_0;
-            acc[52] += (double)v9_8_0;
-            acc[53] += (double)v9_9_0;
-            acc[54] += (double)v10_1_0;
-            acc[55] += (double)v10_2_0;
-            acc[56] += (double)v10_3_0;
-            acc[57] += (double)v10_4_0;
-            acc[58] += (double)v10_5_0;
-            acc[59] += (double)v10_6_0;
-            acc[60] += (double)v10_7_0;
-            acc[61] += (double)v10_8_0;
-            acc[62] += (double)v10_9_0;
-            acc[63] += (double)v11_1_0;
-            acc[64] += (double)v11_2_0;
-            acc[65] += (double)v11_3_0;
-            acc[66] += (double)v11_4_0;
-            acc[67] += (double)v11_5_0;
-            acc[68] += (double)v11_6_0;
-            acc[69] += (double)v11_7_0;
-            acc[70] += (double)v11_8_0;
-            acc[71] += (double)v11_9_0;
-            acc[72] += (double)v12_1_0;
-            acc[73] += (double)v12_2_0;
-            acc[74] += (double)v12_3_0;
-            acc[75] += (double)v12_4_0;
-            acc[76] += (double)v12_5_0;
-            acc[77] += (double)v12_6_0;
-            acc[78] += (double)v12_7_0;
-            acc[79] += (double)v12_8_0;
-            acc[80] += (double)v12_9_0;
-            acc[81] += (double)v13_1_0;
-            acc[82] += (double)v13_2_0;
-            acc[83] += (double)v13_3_0;
-            acc[84] += (double)v13_4_0;
-            acc[85] += (double)v13_5_0;
-            acc[86] += (double)v13_6_0;
-            acc[87] += (double)v13_7_0;
-            acc[88] += (double)v13_8_0;
-            acc[89] += (double)v13_9_0;
-            acc[90] += (double)v14_1_0;
-            acc[91] += (double)v14_2_0;
-            acc[92] += (double)v14_3_0;
-            acc[93] += (double)v14_4_0;
-            acc[94] += (double)v14_5_0;
-            acc[95] += (double)v14_6_0;
-            acc[96] += (double)v14_7_0;
-            acc[97] += (double)v14_8_0;
-            acc[98] += (double)v14_9_0;
-            acc[99] += (double)v15_1_0;
-            acc[100] += (double)v15_2_0;
-            acc[101] += (double)v15_3_0;
-            acc[102] += (double)v15_4_0;
-            acc[103] += (double)v15_5_0;
-            acc[104] += (double)v15_6_0;
-            acc[105] += (double)v15_7_0;
-            acc[106] += (double)v15_8_0;
-            acc[107] += (double)v15_9_0;
-            acc[108] += (double)v16_1_0;
-            acc[109] += (double)v16_2_0;
-            acc[110] += (double)v16_3_0;
-            acc[111] += (double)v16_4_0;
-            acc[112] += (double)v16_5_0;
-            acc[113] += (double)v16_6_0;
-            acc[114] += (double)v16_7_0;
-            acc[115] += (double)v16_8_0;
-            acc[116] += (double)v16_9_0;
-            acc[117] += (double)v17_1_0;
-            acc[118] += (double)v17_2_0;
-            acc[119] += (double)v17_3_0;
-            acc[120] += (double)v17_4_0;
-            acc[121] += (double)v17_5_0;
-            acc[122] += (double)v17_6_0;
-            acc[123] += (double)v17_7_0;
-            acc[124] += (double)v17_8_0;
-            acc[125] += (double)v17_9_0;
-            acc[126] += (double)v18_1_0;
-            acc[127] += (double)v18_2_0;
-            acc[128] += (double)v18_3_0;
-            acc[129] += (double)v18_4_0;
-            acc[130] += (double)v18_5_0;
-            acc[131] += (double)v18_6_0;
-            acc[132] += (double)v18_7_0;
-            acc[133] += (double)v18_8_0;
-            acc[134] += (double)v18_9_0;
-            acc[135] += (double)v19_1_0;
-            acc[136] += (double)v19_2_0;
-            acc[137] += (double)v19_3_0;
-            acc[138] += (double)v19_4_0;
-            acc[139] += (double)v19_5_0;
-            acc[140] += (double)v19_6_0;
-            acc[141] += (double)v19_7_0;
-            acc[142] += (double)v19_8_0;
-            acc[143] += (double)v19_9_0;
+            if constexpr (sizeof(VT) == 8) {
+                acc[0] += (double)v4_1_0;
+                acc[1] += (double)v4_2_0;
+                acc[2] += (double)v4_3_0;
+                acc[3] = fma(QCx, v4_1_0, fma(WQx, v4_1_1, fma(2.0 * oo2ze, v1_1_1, fma(1.0 * oo2e, (v4_0_0 - rho_e * v4_0_1), acc[3]))));
+                acc[4] = fma(QCx, v4_2_0, fma(WQx, v4_2_1, fma(2.0 * oo2ze, v1_2_1, acc[4])));
+                acc[5] = fma(QCx, v4_3_0, fma(WQx, v4_3_1, fma(2.0 * oo2ze, v1_3_1, acc[5])));
+                acc[6] = fma(QCy, v4_2_0, fma(WQy, v4_2_1, fma(1.0 * oo2e, (v4_0_0 - rho_e * v4_0_1), acc[6])));
+                acc[7] = fma(QCy, v4_3_0, fma(WQy, v4_3_1, acc[7]));
+                acc[8] = fma(QCz, v4_3_0, fma(WQz, v4_3_1, fma(1.0 * oo2e, (v4_0_0 - rho_e * v4_0_1), acc[8])));
+                acc[9] += (double)v5_1_0;
+                acc[10] += (double)v5_2_0;
+                acc[11] += (double)v5_3_0;
+                acc[12] = fma(QCx, v5_1_0, fma(WQx, v5_1_1, fma(1.0 * oo2ze, v2_1_1, fma(1.0 * oo2e, (v5_0_0 - rho_e * v5_0_1), acc[12]))));
+                acc[13] = fma(QCx, v5_2_0, fma(WQx, v5_2_1, fma(1.0 * oo2ze, v2_2_1, acc[13])));
+                acc[14] = fma(QCx, v5_3_0, fma(WQx, v5_3_1, fma(1.0 * oo2ze, v2_3_1, acc[14])));
+                acc[15] = fma(QCy, v5_2_0, fma(WQy, v5_2_1, fma(1.0 * oo2ze, v1_2_1, fma(1.0 * oo2e, (v5_0_0 - rho_e * v5_0_1), acc[15]))));
+                acc[16] = fma(QCy, v5_3_0, fma(WQy, v5_3_1, fma(1.0 * oo2ze, v1_3_1, acc[16])));
+                acc[17] = fma(QCz, v5_3_0, fma(WQz, v5_3_1, fma(1.0 * oo2e, (v5_0_0 - rho_e * v5_0_1), acc[17])));
+                acc[18] += (double)v6_1_0;
+                acc[19] += (double)v6_2_0;
+                acc[20] += (double)v6_3_0;
+                acc[21] = fma(QCx, v6_1_0, fma(WQx, v6_1_1, fma(1.0 * oo2ze, v3_1_1, fma(1.0 * oo2e, (v6_0_0 - rho_e * v6_0_1), acc[21]))));
+                acc[22] = fma(QCx, v6_2_0, fma(WQx, v6_2_1, fma(1.0 * oo2ze, v3_2_1, acc[22])));
+                acc[23] = fma(QCx, v6_3_0, fma(WQx, v6_3_1, fma(1.0 * oo2ze, v3_3_1, acc[23])));
+                acc[24] = fma(QCy, v6_2_0, fma(WQy, v6_2_1, fma(1.0 * oo2e, (v6_0_0 - rho_e * v6_0_1), acc[24])));
+                acc[25] = fma(QCy, v6_3_0, fma(WQy, v6_3_1, acc[25]));
+                acc[26] = fma(QCz, v6_3_0, fma(WQz, v6_3_1, fma(1.0 * oo2ze, v1_3_1, fma(1.0 * oo2e, (v6_0_0 - rho_e * v6_0_1), acc[26]))));
+                acc[27] += (double)v7_1_0;
+                acc[28] += (double)v7_2_0;
+                acc[29] += (double)v7_3_0;
+                acc[30] = fma(QCx, v7_1_0, fma(WQx, v7_1_1, fma(1.0 * oo2e, (v7_0_0 - rho_e * v7_0_1), acc[30])));
+                acc[31] = fma(QCx, v7_2_0, fma(WQx, v7_2_1, acc[31]));
+                acc[32] = fma(QCx, v7_3_0, fma(WQx, v7_3_1, acc[32]));
+                acc[33] = fma(QCy, v7_2_0, fma(WQy, v7_2_1, fma(2.0 * oo2ze, v2_2_1, fma(1.0 * oo2e, (v7_0_0 - rho_e * v7_0_1), acc[33]))));
+                acc[34] = fma(QCy, v7_3_0, fma(WQy, v7_3_1, fma(2.0 * oo2ze, v2_3_1, acc[34])));
+                acc[35] = fma(QCz, v7_3_0, fma(WQz, v7_3_1, fma(1.0 * oo2e, (v7_0_0 - rho_e * v7_0_1), acc[35])));
+                acc[36] += (double)v8_1_0;
+                acc[37] += (double)v8_2_0;
+                acc[38] += (double)v8_3_0;
+                acc[39] = fma(QCx, v8_1_0, fma(WQx, v8_1_1, fma(1.0 * oo2e, (v8_0_0 - rho_e * v8_0_1), acc[39])));
+                acc[40] = fma(QCx, v8_2_0, fma(WQx, v8_2_1, acc[40]));
+                acc[41] = fma(QCx, v8_3_0, fma(WQx, v8_3_1, acc[41]));
+                acc[42] = fma(QCy, v8_2_0, fma(WQy, v8_2_1, fma(1.0 * oo2ze, v3_2_1, fma(1.0 * oo2e, (v8_0_0 - rho_e * v8_0_1), acc[42]))));
+                acc[43] = fma(QCy, v8_3_0, fma(WQy, v8_3_1, fma(1.0 * oo2ze, v3_3_1, acc[43])));
+                acc[44] = fma(QCz, v8_3_0, fma(WQz, v8_3_1, fma(1.0 * oo2ze, v2_3_1, fma(1.0 * oo2e, (v8_0_0 - rho_e * v8_0_1), acc[44]))));
+                acc[45] += (double)v9_1_0;
+                acc[46] += (double)v9_2_0;
+                acc[47] += (double)v9_3_0;
+                acc[48] = fma(QCx, v9_1_0, fma(WQx, v9_1_1, fma(1.0 * oo2e, (v9_0_0 - rho_e * v9_0_1), acc[48])));
+                acc[49] = fma(QCx, v9_2_0, fma(WQx, v9_2_1, acc[49]));
+                acc[50] = fma(QCx, v9_3_0, fma(WQx, v9_3_1, acc[50]));
+                acc[51] = fma(QCy, v9_2_0, fma(WQy, v9_2_1, fma(1.0 * oo2e, (v9_0_0 - rho_e * v9_0_1), acc[51])));
+                acc[52] = fma(QCy, v9_3_0, fma(WQy, v9_3_1, acc[52]));
+                acc[53] = fma(QCz, v9_3_0, fma(WQz, v9_3_1, fma(2.0 * oo2ze, v3_3_1, fma(1.0 * oo2e, (v9_0_0 - rho_e * v9_0_1), acc[53]))));
+                acc[54] += (double)v10_1_0;
+                acc[55] += (double)v10_2_0;
+                acc[56] += (double)v10_3_0;
+                acc[57] = fma(QCx, v10_1_0, fma(WQx, v10_1_1, fma(3.0 * oo2ze, v4_1_1, fma(1.0 * oo2e, (v10_0_0 - rho_e * v10_0_1), acc[57]))));
+                acc[58] = fma(QCx, v10_2_0, fma(WQx, v10_2_1, fma(3.0 * oo2ze, v4_2_1, acc[58])));
+                acc[59] = fma(QCx, v10_3_0, fma(WQx, v10_3_1, fma(3.0 * oo2ze, v4_3_1, acc[59])));
+                acc[60] = fma(QCy, v10_2_0, fma(WQy, v10_2_1, fma(1.0 * oo2e, (v10_0_0 - rho_e * v10_0_1), acc[60])));
+                acc[61] = fma(QCy, v10_3_0, fma(WQy, v10_3_1, acc[61]));
+                acc[62] = fma(QCz, v10_3_0, fma(WQz, v10_3_1, fma(1.0 * oo2e, (v10_0_0 - rho_e * v10_0_1), acc[62])));
+                acc[63] += (double)v11_1_0;
+                acc[64] += (double)v11_2_0;
+                acc[65] += (double)v11_3_0;
+                acc[66] = fma(QCx, v11_1_0, fma(WQx, v11_1_1, fma(2.0 * oo2ze, v5_1_1, fma(1.0 * oo2e, (v11_0_0 - rho_e * v11_0_1), acc[66]))));
+                acc[67] = fma(QCx, v11_2_0, fma(WQx, v11_2_1, fma(2.0 * oo2ze, v5_2_1, acc[67])));
+                acc[68] = fma(QCx, v11_3_0, fma(WQx, v11_3_1, fma(2.0 * oo2ze, v5_3_1, acc[68])));
+                acc[69] = fma(QCy, v11_2_0, fma(WQy, v11_2_1, fma(1.0 * oo2ze, v4_2_1, fma(1.0 * oo2e, (v11_0_0 - rho_e * v11_0_1), acc[69]))));
+                acc[70] = fma(QCy, v11_3_0, fma(WQy, v11_3_1, fma(1.0 * oo2ze, v4_3_1, acc[70])));
+                acc[71] = fma(QCz, v11_3_0, fma(WQz, v11_3_1, fma(1.0 * oo2e, (v11_0_0 - rho_e * v11_0_1), acc[71])));
+                acc[72] += (double)v12_1_0;
+                acc[73] += (double)v12_2_0;
+                acc[74] += (double)v12_3_0;
+                acc[75] = fma(QCx, v12_1_0, fma(WQx, v12_1_1, fma(2.0 * oo2ze, v6_1_1, fma(1.0 * oo2e, (v12_0_0 - rho_e * v12_0_1), acc[75]))));
+                acc[76] = fma(QCx, v12_2_0, fma(WQx, v12_2_1, fma(2.0 * oo2ze, v6_2_1, acc[76])));
+                acc[77] = fma(QCx, v12_3_0, fma(WQx, v12_3_1, fma(2.0 * oo2ze, v6_3_1, acc[77])));
+                acc[78] = fma(QCy, v12_2_0, fma(WQy, v12_2_1, fma(1.0 * oo2e, (v12_0_0 - rho_e * v12_0_1), acc[78])));
+                acc[79] = fma(QCy, v12_3_0, fma(WQy, v12_3_1, acc[79]));
+                acc[80] = fma(QCz, v12_3_0, fma(WQz, v12_3_1, fma(1.0 * oo2ze, v4_3_1, fma(1.0 * oo2e, (v12_0_0 - rho_e * v12_0_1), acc[80]))));
+                acc[81] += (double)v13_1_0;
+                acc[82] += (double)v13_2_0;
+                acc[83] += (double)v13_3_0;
+                acc[84] = fma(QCx, v13_1_0, fma(WQx, v13_1_1, fma(1.0 * oo2ze, v7_1_1, fma(1.0 * oo2e, (v13_0_0 - rho_e * v13_0_1), acc[84]))));
+                acc[85] = fma(QCx, v13_2_0, fma(WQx, v13_2_1, fma(1.0 * oo2ze, v7_2_1, acc[85])));
+                acc[86] = fma(QCx, v13_3_0, fma(WQx, v13_3_1, fma(1.0 * oo2ze, v7_3_1, acc[86])));
+                acc[87] = fma(QCy, v13_2_0, fma(WQy, v13_2_1, fma(2.0 * oo2ze, v5_2_1, fma(1.0 * oo2e, (v13_0_0 - rho_e * v13_0_1), acc[87]))));
+                acc[88] = fma(QCy, v13_3_0, fma(WQy, v13_3_1, fma(2.0 * oo2ze, v5_3_1, acc[88])));
+                acc[89] = fma(QCz, v13_3_0, fma(WQz, v13_3_1, fma(1.0 * oo2e, (v13_0_0 - rho_e * v13_0_1), acc[89])));
+                acc[90] += (double)v14_1_0;
+                acc[91] += (double)v14_2_0;
+                acc[92] += (double)v14_3_0;
+                acc[93] = fma(QCx, v14_1_0, fma(WQx, v14_1_1, fma(1.0 * oo2ze, v9_1_1, fma(1.0 * oo2e, (v14_0_0 - rho_e * v14_0_1), acc[93]))));
+                acc[94] = fma(QCx, v14_2_0, fma(WQx, v14_2_1, fma(1.0 * oo2ze, v9_2_1, acc[94])));
+                acc[95] = fma(QCx, v14_3_0, fma(WQx, v14_3_1, fma(1.0 * oo2ze, v9_3_1, acc[95])));
+                acc[96] = fma(QCy, v14_2_0, fma(WQy, v14_2_1, fma(1.0 * oo2e, (v14_0_0 - rho_e * v14_0_1), acc[96])));
+                acc[97] = fma(QCy, v14_3_0, fma(WQy, v14_3_1, acc[97]));
+                acc[98] = fma(QCz, v14_3_0, fma(WQz, v14_3_1, fma(2.0 * oo2ze, v6_3_1, fma(1.0 * oo2e, (v14_0_0 - rho_e * v14_0_1), acc[98]))));
+                acc[99] += (double)v15_1_0;
+                acc[100] += (double)v15_2_0;
+                acc[101] += (double)v15_3_0;
+                acc[102] = fma(QCx, v15_1_0, fma(WQx, v15_1_1, fma(1.0 * oo2ze, v8_1_1, fma(1.0 * oo2e, (v15_0_0 - rho_e * v15_0_1), acc[102]))));
+                acc[103] = fma(QCx, v15_2_0, fma(WQx, v15_2_1, fma(1.0 * oo2ze, v8_2_1, acc[103])));
+                acc[104] = fma(QCx, v15_3_0, fma(WQx, v15_3_1, fma(1.0 * oo2ze, v8_3_1, acc[104])));
+                acc[105] = fma(QCy, v15_2_0, fma(WQy, v15_2_1, fma(1.0 * oo2ze, v6_2_1, fma(1.0 * oo2e, (v15_0_0 - rho_e * v15_0_1), acc[105]))));
+                acc[106] = fma(QCy, v15_3_0, fma(WQy, v15_3_1, fma(1.0 * oo2ze, v6_3_1, acc[106])));
+                acc[107] = fma(QCz, v15_3_0, fma(WQz, v15_3_1, fma(1.0 * oo2ze, v5_3_1, fma(1.0 * oo2e, (v15_0_0 - rho_e * v15_0_1), acc[107]))));
+                acc[108] += (double)v16_1_0;
+                acc[109] += (double)v16_2_0;
+                acc[110] += (double)v16_3_0;
+                acc[111] = fma(QCx, v16_1_0, fma(WQx, v16_1_1, fma(1.0 * oo2e, (v16_0_0 - rho_e * v16_0_1), acc[111])));
+                acc[112] = fma(QCx, v16_2_0, fma(WQx, v16_2_1, acc[112]));
+                acc[113] = fma(QCx, v16_3_0, fma(WQx, v16_3_1, acc[113]));
+                acc[114] = fma(QCy, v16_2_0, fma(WQy, v16_2_1, fma(3.0 * oo2ze, v7_2_1, fma(1.0 * oo2e, (v16_0_0 - rho_e * v16_0_1), acc[114]))));
+                acc[115] = fma(QCy, v16_3_0, fma(WQy, v16_3_1, fma(3.0 * oo2ze, v7_3_1, acc[115])));
+                acc[116] = fma(QCz, v16_3_0, fma(WQz, v16_3_1, fma(1.0 * oo2e, (v16_0_0 - rho_e * v16_0_1), acc[116])));
+                acc[117] += (double)v17_1_0;
+                acc[118] += (double)v17_2_0;
+                acc[119] += (double)v17_3_0;
+                acc[120] = fma(QCx, v17_1_0, fma(WQx, v17_1_1, fma(1.0 * oo2e, (v17_0_0 - rho_e * v17_0_1), acc[120])));
+                acc[121] = fma(QCx, v17_2_0, fma(WQx, v17_2_1, acc[121]));
+                acc[122] = fma(QCx, v17_3_0, fma(WQx, v17_3_1, acc[122]));
+                acc[123] = fma(QCy, v17_2_0, fma(WQy, v17_2_1, fma(2.0 * oo2ze, v8_2_1, fma(1.0 * oo2e, (v17_0_0 - rho_e * v17_0_1), acc[123]))));
+                acc[124] = fma(QCy, v17_3_0, fma(WQy, v17_3_1, fma(2.0 * oo2ze, v8_3_1, acc[124])));
+                acc[125] = fma(QCz, v17_3_0, fma(WQz, v17_3_1, fma(1.0 * oo2ze, v7_3_1, fma(1.0 * oo2e, (v17_0_0 - rho_e * v17_0_1), acc[125]))));
+                acc[126] += (double)v18_1_0;
+                acc[127] += (double)v18_2_0;
+                acc[128] += (double)v18_3_0;
+                acc[129] = fma(QCx, v18_1_0, fma(WQx, v18_1_1, fma(1.0 * oo2e, (v18_0_0 - rho_e * v18_0_1), acc[129])));
+                acc[130] = fma(QCx, v18_2_0, fma(WQx, v18_2_1, acc[130]));
+                acc[131] = fma(QCx, v18_3_0, fma(WQx, v18_3_1, acc[131]));
+                acc[132] = fma(QCy, v18_2_0, fma(WQy, v18_2_1, fma(1.0 * oo2ze, v9_2_1, fma(1.0 * oo2e, (v18_0_0 - rho_e * v18_0_1), acc[132]))));
+                acc[133] = fma(QCy, v18_3_0, fma(WQy, v18_3_1, fma(1.0 * oo2ze, v9_3_1, acc[133])));
+                acc[134] = fma(QCz, v18_3_0, fma(WQz, v18_3_1, fma(2.0 * oo2ze, v8_3_1, fma(1.0 * oo2e, (v18_0_0 - rho_e * v18_0_1), acc[134]))));
+                acc[135] += (double)v19_1_0;
+                acc[136] += (double)v19_2_0;
+                acc[137] += (double)v19_3_0;
+                acc[138] = fma(QCx, v19_1_0, fma(WQx, v19_1_1, fma(1.0 * oo2e, (v19_0_0 - rho_e * v19_0_1), acc[138])));
+                acc[139] = fma(QCx, v19_2_0, fma(WQx, v19_2_1, acc[139]));
+                acc[140] = fma(QCx, v19_3_0, fma(WQx, v19_3_1, acc[140]));
+                acc[141] = fma(QCy, v19_2_0, fma(WQy, v19_2_1, fma(1.0 * oo2e, (v19_0_0 - rho_e * v19_0_1), acc[141])));
+                acc[142] = fma(QCy, v19_3_0, fma(WQy, v19_3_1, acc[142]));
+                acc[143] = fma(QCz, v19_3_0, fma(WQz, v19_3_1, fma(3.0 * oo2ze, v9_3_1, fma(1.0 * oo2e, (v19_0_0 - rho_e * v19_0_1), acc[143]))));
+            } else {
+                acc[0] += (double)v4_1_0;
+                acc[1] += (double)v4_2_0;
+                acc[2] += (double)v4_3_0;
+                const VT v4_4_0 = QCx * v4_1_0 + WQx * v4_1_1 + (VT)2.0 * oo2ze * v1_1_1 + (VT)1.0 * oo2e * (v4_0_0 - rho_e * v4_0_1);
+                acc[3] += (double)v4_4_0;
+                const VT v4_5_0 = QCx * v4_2_0 + WQx * v4_2_1 + (VT)2.0 * oo2ze * v1_2_1;
+                acc[4] += (double)v4_5_0;
+                const VT v4_6_0 = QCx * v4_3_0 + WQx * v4_3_1 + (VT)2.0 * oo2ze * v1_3_1;
+                acc[5] += (double)v4_6_0;
+                const VT v4_7_0 = QCy * v4_2_0 + WQy * v4_2_1 + (VT)1.0 * oo2e * (v4_0_0 - rho_e * v4_0_1);
+                acc[6] += (double)v4_7_0;
+                const VT v4_8_0 = QCy * v4_3_0 + WQy * v4_3_1;
+                acc[7] += (double)v4_8_0;
+                const VT v4_9_0 = QCz * v4_3_0 + WQz * v4_3_1 + (VT)1.0 * oo2e * (v4_0_0 - rho_e * v4_0_1);
+                acc[8] += (double)v4_9_0;
+                acc[9] += (double)v5_1_0;
+                acc[10] += (double)v5_2_0;
+                acc[11] += (double)v5_3_0;
+                const VT v5_4_0 = QCx * v5_1_0 + WQx * v5_1_1 + (VT)1.0 * oo2ze * v2_1_1 + (VT)1.0 * oo2e * (v5_0_0 - rho_e * v5_0_1);
+                acc[12] += (double)v5_4_0;
+                const VT v5_5_0 = QCx * v5_2_0 + WQx * v5_2_1 + (VT)1.0 * oo2ze * v2_2_1;
+                acc[13] += (double)v5_5_0;
+                const VT v5_6_0 = QCx * v5_3_0 + WQx * v5_3_1 + (VT)1.0 * oo2ze * v2_3_1;
+                acc[14] += (double)v5_6_0;
+                const VT v5_7_0 = QCy * v5_2_0 + WQy * v5_2_1 + (VT)1.0 * oo2ze * v1_2_1 + (VT)1.0 * oo2e * (v5_0_0 - rho_e * v5_0_1);
+                acc[15] += (double)v5_7_0;
+                const VT v5_8_0 = QCy * v5_3_0 + WQy * v5_3_1 + (VT)1.0 * oo2ze * v1_3_1;
+                acc[16] += (double)v5_8_0;
+                const VT v5_9_0 = QCz * v5_3_0 + WQz * v5_3_1 + (VT)1.0 * oo2e * (v5_0_0 - rho_e * v5_0_1);
+                acc[17] += (double)v5_9_0;
+                acc[18] += (double)v6_1_0;
+                acc[19] += (double)v6_2_0;
+                acc[20] += (double)v6_3_0;
+                const VT v6_4_0 = QCx * v6_1_0 + WQx * v6_1_1 + (VT)1.0 * oo2ze * v3_1_1 + (VT)1.0 * oo2e * (v6_0_0 - rho_e * v6_0_1);
+                acc[21] += (double)v6_4_0;
+                const VT v6_5_0 = QCx * v6_2_0 + WQx * v6_2_1 + (VT)1.0 * oo2ze * v3_2_1;
+                acc[22] += (double)v6_5_0;
+                const VT v6_6_0 = QCx * v6_3_0 + WQx * v6_3_1 + (VT)1.0 * oo2ze * v3_3_1;
+                acc[23] += (double)v6_6_0;
+                const VT v6_7_0 = QCy * v6_2_0 + WQy * v6_2_1 + (VT)1.0 * oo2e * (v6_0_0 - rho_e * v6_0_1);
+                acc[24] += (double)v6_7_0;
+                const VT v6_8_0 = QCy * v6_3_0 + WQy * v6_3_1;
+                acc[25] += (double)v6_8_0;
+                const VT v6_9_0 = QCz * v6_3_0 + WQz * v6_3_1 + (VT)1.0 * oo2ze * v1_3_1 + (VT)1.0 * oo2e * (v6_0_0 - rho_e * v6_0_1);
+                acc[26] += (double)v6_9_0;
+                acc[27] += (double)v7_1_0;
+                acc[28] += (double)v7_2_0;
+                acc[29] += (double)v7_3_0;
+                const VT v7_4_0 = QCx * v7_1_0 + WQx * v7_1_1 + (VT)1.0 * oo2e * (v7_0_0 - rho_e * v7_0_1);
+                acc[30] += (double)v7_4_0;
+                const VT v7_5_0 = QCx * v7_2_0 + WQx * v7_2_1;
+                acc[31] += (double)v7_5_0;
+                const VT v7_6_0 = QCx * v7_3_0 + WQx * v7_3_1;
+                acc[32] += (double)v7_6_0;
+                const VT v7_7_0 = QCy * v7_2_0 + WQy * v7_2_1 + (VT)2.0 * oo2ze * v2_2_1 + (VT)1.0 * oo2e * (v7_0_0 - rho_e * v7_0_1);
+                acc[33] += (double)v7_7_0;
+                const VT v7_8_0 = QCy * v7_3_0 + WQy * v7_3_1 + (VT)2.0 * oo2ze * v2_3_1;
+                acc[34] += (double)v7_8_0;
+                const VT v7_9_0 = QCz * v7_3_0 + WQz * v7_3_1 + (VT)1.0 * oo2e * (v7_0_0 - rho_e * v7_0_1);
+                acc[35] += (double)v7_9_0;
+                acc[36] += (double)v8_1_0;
+                acc[37] += (double)v8_2_0;
+                acc[38] += (double)v8_3_0;
+                const VT v8_4_0 = QCx * v8_1_0 + WQx * v8_1_1 + (VT)1.0 * oo2e * (v8_0_0 - rho_e * v8_0_1);
+                acc[39] += (double)v8_4_0;
+                const VT v8_5_0 = QCx * v8_2_0 + WQx * v8_2_1;
+                acc[40] += (double)v8_5_0;
+                const VT v8_6_0 = QCx * v8_3_0 + WQx * v8_3_1;
+                acc[41] += (double)v8_6_0;
+                const VT v8_7_0 = QCy * v8_2_0 + WQy * v8_2_1 + (VT)1.0 * oo2ze * v3_2_1 + (VT)1.0 * oo2e * (v8_0_0 - rho_e * v8_0_1);
+                acc[42] += (double)v8_7_0;
+                const VT v8_8_0 = QCy * v8_3_0 + WQy * v8_3_1 + (VT)1.0 * oo2ze * v3_3_1;
+                acc[43] += (double)v8_8_0;
+                const VT v8_9_0 = QCz * v8_3_0 + WQz * v8_3_1 + (VT)1.0 * oo2ze * v2_3_1 + (VT)1.0 * oo2e * (v8_0_0 - rho_e * v8_0_1);
+                acc[44] += (double)v8_9_0;
+                acc[45] += (double)v9_1_0;
+                acc[46] += (double)v9_2_0;
+                acc[47] += (double)v9_3_0;
+                const VT v9_4_0 = QCx * v9_1_0 + WQx * v9_1_1 + (VT)1.0 * oo2e * (v9_0_0 - rho_e * v9_0_1);
+                acc[48] += (double)v9_4_0;
+                const VT v9_5_0 = QCx * v9_2_0 + WQx * v9_2_1;
+                acc[49] += (double)v9_5_0;
+                const VT v9_6_0 = QCx * v9_3_0 + WQx * v9_3_1;
+                acc[50] += (double)v9_6_0;
+                const VT v9_7_0 = QCy * v9_2_0 + WQy * v9_2_1 + (VT)1.0 * oo2e * (v9_0_0 - rho_e * v9_0_1);
+                acc[51] += (double)v9_7_0;
+                const VT v9_8_0 = QCy * v9_3_0 + WQy * v9_3_1;
+                acc[52] += (double)v9_8_0;
+                const VT v9_9_0 = QCz * v9_3_0 + WQz * v9_3_1 + (VT)2.0 * oo2ze * v3_3_1 + (VT)1.0 * oo2e * (v9_0_0 - rho_e * v9_0_1);
+                acc[53] += (double)v9_9_0;
+                acc[54] += (double)v10_1_0;
+                acc[55] += (double)v10_2_0;
+                acc[56] += (double)v10_3_0;
+                const VT v10_4_0 = QCx * v10_1_0 + WQx * v10_1_1 + (VT)3.0 * oo2ze * v4_1_1 + (VT)1.0 * oo2e * (v10_0_0 - rho_e * v10_0_1);
+                acc[57] += (double)v10_4_0;
+                const VT v10_5_0 = QCx * v10_2_0 + WQx * v10_2_1 + (VT)3.0 * oo2ze * v4_2_1;
+                acc[58] += (double)v10_5_0;
+                const VT v10_6_0 = QCx * v10_3_0 + WQx * v10_3_1 + (VT)3.0 * oo2ze * v4_3_1;
+                acc[59] += (double)v10_6_0;
+                const VT v10_7_0 = QCy * v10_2_0 + WQy * v10_2_1 + (VT)1.0 * oo2e * (v10_0_0 - rho_e * v10_0_1);
+                acc[60] += (double)v10_7_0;
+                const VT v10_8_0 = QCy * v10_3_0 + WQy * v10_3_1;
+                acc[61] += (double)v10_8_0;
+                const VT v10_9_0 = QCz * v10_3_0 + WQz * v10_3_1 + (VT)1.0 * oo2e * (v10_0_0 - rho_e * v10_0_1);
+                acc[62] += (double)v10_9_0;
+                acc[63] += (double)v11_1_0;
+                acc[64] += (double)v11_2_0;
+                acc[65] += (double)v11_3_0;
+                const VT v11_4_0 = QCx * v11_1_0 + WQx * v11_1_1 + (VT)2.0 * oo2ze * v5_1_1 + (VT)1.0 * oo2e * (v11_0_0 - rho_e * v11_0_1);
+                acc[66] += (double)v11_4_0;
+                const VT v11_5_0 = QCx * v11_2_0 + WQx * v11_2_1 + (VT)2.0 * oo2ze * v5_2_1;
+                acc[67] += (double)v11_5_0;
+                const VT v11_6_0 = QCx * v11_3_0 + WQx * v11_3_1 + (VT)2.0 * oo2ze * v5_3_1;
+                acc[68] += (double)v11_6_0;
+                const VT v11_7_0 = QCy * v11_2_0 + WQy * v11_2_1 + (VT)1.0 * oo2ze * v4_2_1 + (VT)1.0 * oo2e * (v11_0_0 - rho_e * v11_0_1);
+                acc[69] += (double)v11_7_0;
+                const VT v11_8_0 = QCy * v11_3_0 + WQy * v11_3_1 + (VT)1.0 * oo2ze * v4_3_1;
+                acc[70] += (double)v11_8_0;
+                const VT v11_9_0 = QCz * v11_3_0 + WQz * v11_3_1 + (VT)1.0 * oo2e * (v11_0_0 - rho_e * v11_0_1);
+                acc[71] += (double)v11_9_0;
+                acc[72] += (double)v12_1_0;
+                acc[73] += (double)v12_2_0;
+                acc[74] += (double)v12_3_0;
+                const VT v12_4_0 = QCx * v12_1_0 + WQx * v12_1_1 + (VT)2.0 * oo2ze * v6_1_1 + (VT)1.0 * oo2e * (v12_0_0 - rho_e * v12_0_1);
+                acc[75] += (double)v12_4_0;
+                const VT v12_5_0 = QCx * v12_2_0 + WQx * v12_2_1 + (VT)2.0 * oo2ze * v6_2_1;
+                acc[76] += (double)v12_5_0;
+                const VT v12_6_0 = QCx * v12_3_0 + WQx * v12_3_1 + (VT)2.0 * oo2ze * v6_3_1;
+                acc[77] += (double)v12_6_0;
+                const VT v12_7_0 = QCy * v12_2_0 + WQy * v12_2_1 + (VT)1.0 * oo2e * (v12_0_0 - rho_e * v12_0_1);
+                acc[78] += (double)v12_7_0;
+                const VT v12_8_0 = QCy * v12_3_0 + WQy * v12_3_1;
+                acc[79] += (double)v12_8_0;
+                const VT v12_9_0 = QCz * v12_3_0 + WQz * v12_3_1 + (VT)1.0 * oo2ze * v4_3_1 + (VT)1.0 * oo2e * (v12_0_0 - rho_e * v12_0_1);
+                acc[80] += (double)v12_9_0;
+                acc[81] += (double)v13_1_0;
+                acc[82] += (double)v13_2_0;
+                acc[83] += (double)v13_3_0;
+                const VT v13_4_0 = QCx * v13_1_0 + WQx * v13_1_1 + (VT)1.0 * oo2ze * v7_1_1 + (VT)1.0 * oo2e * (v13_0_0 - rho_e * v13_0_1);
+                acc[84] += (double)v13_4_0;
+                const VT v13_5_0 = QCx * v13_2_0 + WQx * v13_2_1 + (VT)1.0 * oo2ze * v7_2_1;
+                acc[85] += (double)v13_5_0;
+                const VT v13_6_0 = QCx * v13_3_0 + WQx * v13_3_1 + (VT)1.0 * oo2ze * v7_3_1;
+                acc[86] += (double)v13_6_0;
+                const VT v13_7_0 = QCy * v13_2_0 + WQy * v13_2_1 + (VT)2.0 * oo2ze * v5_2_1 + (VT)1.0 * oo2e * (v13_0_0 - rho_e * v13_0_1);
+                acc[87] += (double)v13_7_0;
+                const VT v13_8_0 = QCy * v13_3_0 + WQy * v13_3_1 + (VT)2.0 * oo2ze * v5_3_1;
+                acc[88] += (double)v13_8_0;
+                const VT v13_9_0 = QCz * v13_3_0 + WQz * v13_3_1 + (VT)1.0 * oo2e * (v13_0_0 - rho_e * v13_0_1);
+                acc[89] += (double)v13_9_0;
+                acc[90] += (double)v14_1_0;
+                acc[91] += (double)v14_2_0;
+                acc[92] += (double)v14_3_0;
+                const VT v14_4_0 = QCx * v14_1_0 + WQx * v14_1_1 + (VT)1.0 * oo2ze * v9_1_1 + (VT)1.0 * oo2e * (v14_0_0 - rho_e * v14_0_1);
+                acc[93] += (double)v14_4_0;
+                const VT v14_5_0 = QCx * v14_2_0 + WQx * v14_2_1 + (VT)1.0 * oo2ze * v9_2_1;
+                acc[94] += (double)v14_5_0;
+                const VT v14_6_0 = QCx * v14_3_0 + WQx * v14_3_1 + (VT)1.0 * oo2ze * v9_3_1;
+                acc[95] += (double)v14_6_0;
+                const VT v14_7_0 = QCy * v14_2_0 + WQy * v14_2_1 + (VT)1.0 * oo2e * (v14_0_0 - rho_e * v14_0_1);
+                acc[96] += (double)v14_7_0;
+                const VT v14_8_0 = QCy * v14_3_0 + WQy * v14_3_1;
+                acc[97] += (double)v14_8_0;
+                const VT v14_9_0 = QCz * v14_3_0 + WQz * v14_3_1 + (VT)2.0 * oo2ze * v6_3_1 + (VT)1.0 * oo2e * (v14_0_0 - rho_e * v14_0_1);
+                acc[98] += (double)v14_9_0;
+                acc[99] += (double)v15_1_0;
+                acc[100] += (double)v15_2_0;
+                acc[101] += (double)v15_3_0;
+                const VT v15_4_0 = QCx * v15_1_0 + WQx * v15_1_1 + (VT)1.0 * oo2ze * v8_1_1 + (VT)1.0 * oo2e * (v15_0_0 - rho_e * v15_0_1);
+                acc[102] += (double)v15_4_0;
+                const VT v15_5_0 = QCx * v15_2_0 + WQx * v15_2_1 + (VT)1.0 * oo2ze * v8_2_1;
+                acc[103] += (double)v15_5_0;
+                const VT v15_6_0 = QCx * v15_3_0 + WQx * v15_3_1 + (VT)1.0 * oo2ze * v8_3_1;
+                acc[104] += (double)v15_6_0;
+                const VT v15_7_0 = QCy * v15_2_0 + WQy * v15_2_1 + (VT)1.0 * oo2ze * v6_2_1 + (VT)1.0 * oo2e * (v15_0_0 - rho_e * v15_0_1);
+                acc[105] += (double)v15_7_0;
+                const VT v15_8_0 = QCy * v15_3_0 + WQy * v15_3_1 + (VT)1.0 * oo2ze * v6_3_1;
+                acc[106] += (double)v15_8_0;
+                const VT v15_9_0 = QCz * v15_3_0 + WQz * v15_3_1 + (VT)1.0 * oo2ze * v5_3_1 + (VT)1.0 * oo2e * (v15_0_0 - rho_e * v15_0_1);
+                acc[107] += (double)v15_9_0;
+                acc[108] += (double)v16_1_0;
+                acc[109] += (double)v16_2_0;
+                acc[110] += (double)v16_3_0;
+                const VT v16_4_0 = QCx * v16_1_0 + WQx * v16_1_1 + (VT)1.0 * oo2e * (v16_0_0 - rho_e * v16_0_1);
+                acc[111] += (double)v16_4_0;
+                const VT v16_5_0 = QCx * v16_2_0 + WQx * v16_2_1;
+                acc[112] += (double)v16_5_0;
+                const VT v16_6_0 = QCx * v16_3_0 + WQx * v16_3_1;
+                acc[113] += (double)v16_6_0;
+                const VT v16_7_0 = QCy * v16_2_0 + WQy * v16_2_1 + (VT)3.0 * oo2ze * v7_2_1 + (VT)1.0 * oo2e * (v16_0_0 - rho_e * v16_0_1);
+                acc[114] += (double)v16_7_0;
+                const VT v16_8_0 = QCy * v16_3_0 + WQy * v16_3_1 + (VT)3.0 * oo2ze * v7_3_1;
+                acc[115] += (double)v16_8_0;
+                const VT v16_9_0 = QCz * v16_3_0 + WQz * v16_3_1 + (VT)1.0 * oo2e * (v16_0_0 - rho_e * v16_0_1);
+                acc[116] += (double)v16_9_0;
+                acc[117] += (double)v17_1_0;
+                acc[118] += (double)v17_2_0;
+                acc[119] += (double)v17_3_0;
+                const VT v17_4_0 = QCx * v17_1_0 + WQx * v17_1_1 + (VT)1.0 * oo2e * (v17_0_0 - rho_e * v17_0_1);
+                acc[120] += (double)v17_4_0;
+                const VT v17_5_0 = QCx * v17_2_0 + WQx * v17_2_1;
+                acc[121] += (double)v17_5_0;
+                const VT v17_6_0 = QCx * v17_3_0 + WQx * v17_3_1;
+                acc[122] += (double)v17_6_0;
+                const VT v17_7_0 = QCy * v17_2_0 + WQy * v17_2_1 + (VT)2.0 * oo2ze * v8_2_1 + (VT)1.0 * oo2e * (v17_0_0 - rho_e * v17_0_1);
+                acc[123] += (double)v17_7_0;
+                const VT v17_8_0 = QCy * v17_3_0 + WQy * v17_3_1 + (VT)2.0 * oo2ze * v8_3_1;
+                acc[124] += (double)v17_8_0;
+                const VT v17_9_0 = QCz * v17_3_0 + WQz * v17_3_1 + (VT)1.0 * oo2ze * v7_3_1 + (VT)1.0 * oo2e * (v17_0_0 - rho_e * v17_0_1);
+                acc[125] += (double)v17_9_0;
+                acc[126] += (double)v18_1_0;
+                acc[127] += (double)v18_2_0;
+                acc[128] += (double)v18_3_0;
+                const VT v18_4_0 = QCx * v18_1_0 + WQx * v18_1_1 + (VT)1.0 * oo2e * (v18_0_0 - rho_e * v18_0_1);
+                acc[129] += (double)v18_4_0;
+                const VT v18_5_0 = QCx * v18_2_0 + WQx * v18_2_1;
+                acc[130] += (double)v18_5_0;
+                const VT v18_6_0 = QCx * v18_3_0 + WQx * v18_3_1;
+                acc[131] += (double)v18_6_0;
+                const VT v18_7_0 = QCy * v18_2_0 + WQy * v18_2_1 + (VT)1.0 * oo2ze * v9_2_1 + (VT)1.0 * oo2e * (v18_0_0 - rho_e * v18_0_1);
+                acc[132] += (double)v18_7_0;
+                const VT v18_8_0 = QCy * v18_3_0 + WQy * v18_3_1 + (VT)1.0 * oo2ze * v9_3_1;
+                acc[133] += (double)v18_8_0;
+                const VT v18_9_0 = QCz * v18_3_0 + WQz * v18_3_1 + (VT)2.0 * oo2ze * v8_3_1 + (VT)1.0 * oo2e * (v18_0_0 - rho_e * v18_0_1);
+                acc[134] += (double)v18_9_0;
+                acc[135] += (double)v19_1_0;
+                acc[136] += (double)v19_2_0;
+                acc[137] += (double)v19_3_0;
+                const VT v19_4_0 = QCx * v19_1_0 + WQx * v19_1_1 + (VT)1.0 * oo2e * (v19_0_0 - rho_e * v19_0_1);
+                acc[138] += (double)v19_4_0;
+                const VT v19_5_0 = QCx * v19_2_0 + WQx * v19_2_1;
+                acc[139] += (double)v19_5_0;
+                const VT v19_6_0 = QCx * v19_3_0 + WQx * v19_3_1;
+                acc[140] += (double)v19_6_0;
+                const VT v19_7_0 = QCy * v19_2_0 + WQy * v19_2_1 + (VT)1.0 * oo2e * (v19_0_0 - rho_e * v19_0_1);
+                acc[141] += (double)v19_7_0;
+                const VT v19_8_0 = QCy * v19_3_0 + WQy * v19_3_1;
+                acc[142] += (double)v19_8_0;
+                const VT v19_9_0 = QCz * v19_3_0 + WQz * v19_3_1 + (VT)3.0 * oo2ze * v9_3_1 + (VT)1.0 * oo2e * (v19_0_0 - rho_e * v19_0_1);
+                acc[143] += (double)v19_9_0;
+            }
         }
     }
 }

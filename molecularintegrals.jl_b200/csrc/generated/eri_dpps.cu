@@ -25,13 +25,13 @@ __device__ __forceinline__ void vrr_dpps(const PairTab &P, const BoysTab &B, int
             const double r = rsqrt(bra.zeta + ket.zeta);
             const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
-            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[5];
             boys_fm<4>(T, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
-            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
             const VT WQx = (VT)(zz * PQx), WQy = (VT)(zz * PQy), WQz = (VT)(zz * PQz);
             const VT oo2z = (VT)bra.oo2z, oo2e = (VT)ket.oo2z, oo2ze = (VT)(0.5 * r2);
@@ -94,102 +94,153 @@ __device__ __forceinline__ void vrr_dpps(const PairTab &P, const BoysTab &B, int
             const VT v18_0_1 = PAz * v8_0_1 + WPz * v8_0_2 + (VT)1.0 * oo2z * (v2_0_1 - rho_z * v2_0_2);
             const VT v19_0_0 = PAz * v9_0_0 + WPz * v9_0_1 + (VT)2.0 * oo2z * (v3_0_0 - rho_z * v3_0_1);
             const VT v19_0_1 = PAz * v9_0_1 + WPz * v9_0_2 + (VT)2.0 * oo2z * (v3_0_1 - rho_z * v3_0_2);
-            const VT v4_1_0 = QCx * v4_0_0 + WQx * v4_0_1 + (VT)2.0 * oo2ze * v1_0_1;
-            const VT v5_1_0 = QCx * v5_0_0 + WQx * v5_0_1 + (VT)1.0 * oo2ze * v2_0_1;
-            const VT v6_1_0 = QCx * v6_0_0 + WQx * v6_0_1 + (VT)1.0 * oo2ze * v3_0_1;
-            const VT v7_1_0 = QCx * v7_0_0 + WQx * v7_0_1;
-            const VT v8_1_0 = QCx * v8_0_0 + WQx * v8_0_1;
-            const VT v9_1_0 = QCx * v9_0_0 + WQx * v9_0_1;
-            const VT v10_1_0 = QCx * v10_0_0 + WQx * v10_0_1 + (VT)3.0 * oo2ze * v4_0_1;
-            const VT v11_1_0 = QCx * v11_0_0 + WQx * v11_0_1 + (VT)2.0 * oo2ze * v5_0_1;
-            const VT v12_1_0 = QCx * v12_0_0 + WQx * v12_0_1 + (VT)2.0 * oo2ze * v6_0_1;
-            const VT v13_1_0 = QCx * v13_0_0 + WQx * v13_0_1 + (VT)1.0 * oo2ze * v7_0_1;
-            const VT v14_1_0 = QCx * v14_0_0 + WQx * v14_0_1 + (VT)1.0 * oo2ze * v9_0_1;
-            const VT v15_1_0 = QCx * v15_0_0 + WQx * v15_0_1 + (VT)1.0 * oo2ze * v8_0_1;
-            const VT v16_1_0 = QCx * v16_0_0 + WQx * v16_0_1;
-            const VT v17_1_0 = QCx * v17_0_0 + WQx * v17_0_1;
-            const VT v18_1_0 = QCx * v18_0_0 + WQx * v18_0_1;
-            const VT v19_1_0 = QCx * v19_0_0 + WQx * v19_0_1;
-            const VT v4_2_0 = QCy * v4_0_0 + WQy * v4_0_1;
-            const VT v5_2_0 = QCy * v5_0_0 + WQy * v5_0_1 + (VT)1.0 * oo2ze * v1_0_1;
-            const VT v6_2_0 = QCy * v6_0_0 + WQy * v6_0_1;
-            const VT v7_2_0 = QCy * v7_0_0 + WQy * v7_0_1 + (VT)2.0 * oo2ze * v2_0_1;
-            const VT v8_2_0 = QCy * v8_0_0 + WQy * v8_0_1 + (VT)1.0 * oo2ze * v3_0_1;
-            const VT v9_2_0 = QCy * v9_0_0 + WQy * v9_0_1;
-            const VT v10_2_0 = QCy * v10_0_0 + WQy * v10_0_1;
-            const VT v11_2_0 = QCy * v11_0_0 + WQy * v11_0_1 + (VT)1.0 * oo2ze * v4_0_1;
-            const VT v12_2_0 = QCy * v12_0_0 + WQy * v12_0_1;
-            const VT v13_2_0 = QCy * v13_0_0 + WQy * v13_0_1 + (VT)2.0 * oo2ze * v5_0_1;
-            const VT v14_2_0 = QCy * v14_0_0 + WQy * v14_0_1;
-            const VT v15_2_0 = QCy * v15_0_0 + WQy * v15_0_1 + (VT)1.0 * oo2ze * v6_0_1;
-            const VT v16_2_0 = QCy * v16_0_0 + WQy * v16_0_1 + (VT)3.0 * oo2ze * v7_0_1;
-            const VT v17_2_0 = QCy * v17_0_0 + WQy * v17_0_1 + (VT)2.0 * oo2ze * v8_0_1;
-            const VT v18_2_0 = QCy * v18_0_0 + WQy * v18_0_1 + (VT)1.0 * oo2ze * v9_0_1;
-            const VT v19_2_0 = QCy * v19_0_0 + WQy * v19_0_1;
-            const VT v4_3_0 = QCz * v4_0_0 + WQz * v4_0_1;
-            const VT v5_3_0 = QCz * v5_0_0 + WQz * v5_0_1;
-            const VT v6_3_0 = QCz * v6_0_0 + WQz * v6_0_1 + (VT)1.0 * oo2ze * v1_0_1;
-            const VT v7_3_0 = QCz * v7_0_0 + WQz * v7_0_1;
-            const VT v8_3_0 = QCz * v8_0_0 + WQz * v8_0_1 + (VT)1.0 * oo2ze * v2_0_1;
-            const VT v9_3_0 = QCz * v9_0_0 + WQz * v9_0_1 + (VT)2.0 * oo2ze * v3_0_1;
-            const VT v10_3_0 = QCz * v10_0_0 + WQz * v10_0_1;
-            const VT v11_3_0 = QCz * v11_0_0 + WQz * v11_0_1;
-            const VT v12_3_0 = QCz * v12_0_0 + WQz * v12_0_1 + (VT)1.0 * oo2ze * v4_0_1;
-            const VT v13_3_0 = QCz * v13_0_0 + WQz * v13_0_1;
-            const VT v14_3_0 = QCz * v14_0_0 + WQz * v14_0_1 + (VT)2.0 * oo2ze * v6_0_1;
-            const VT v15_3_0 = QCz * v15_0_0 + WQz * v15_0_1 + (VT)1.0 * oo2ze * v5_0_1;
-            const VT v16_3_0 = QCz * v16_0_0 + WQz * v16_0_1;
-            const VT v17_3_0 = QCz * v17_0_0 + WQz * v17_0_1 + (VT)1.0 * oo2ze * v7_0_1;
-            const VT v18_3_0 = QCz * v18_0_0 + WQz * v18_0_1 + (VT)2.0 * oo2ze * v8_0_1;
-            const VT v19_3_0 = QCz * v19_0_0 + WQz * v19_0_1 + (VT)3.0 * oo2ze * v9_0_1;
-            acc[0] += (double)v4_1_0;
-            acc[1] += (double)v4_2_0;
-            acc[2] += (double)v4_3_0;
-            acc[3] += (double)v5_1_0;
-            acc[4] += (double)v5_2_0;
-            acc[5] += (double)v5_3_0;
-            acc[6] += (double)v6_1_0;
-            acc[7] += (double)v6_2_0;
-            acc[8] += (double)v6_3_0;
-            acc[9] += (double)v7_1_0;
-            acc[10] += (double)v7_2_0;
-            acc[11] += (double)v7_3_0;
-            acc[12] += (double)v8_1_0;
-            acc[13] += (double)v8_2_0;
-            acc[14] += (double)v8_3_0;
-            acc[15] += (double)v9_1_0;
-            acc[16] += (double)v9_2_0;
-            acc[17] += (double)v9_3_0;
-            acc[18] += (double)v10_1_0;
-            acc[19] += (double)v10_2_0;
-            acc[20] += (double)v10_3_0;
-            acc[21] += (double)v11_1_0;
-            acc[22] += (double)v11_2_0;
-            acc[23] += (double)v11_3_0;
-            acc[24] += (double)v12_1_0;
-            acc[25] += (double)v12_2_0;
-            acc[26] += (double)v12_3_0;
-            acc[27] += (double)v13_1_0;
-            acc[28] += (double)v13_2_0;
-            acc[29] += (double)v13_3_0;
-            acc[30] += (double)v14_1_0;
-            acc[31] += (double)v14_2_0;
-            acc[32] += (double)v14_3_0;
-            acc[33] += (double)v15_1_0;
-            acc[34] += (double)v15_2_0;
-            acc[35] += (double)v15_3_0;
-            acc[36] += (double)v16_1_0;
-            acc[37] += (double)v16_2_0;
-            acc[38] += (double)v16_3_0;
-            acc[39] += (double)v17_1_0;
-            acc[40] += (double)v17_2_0;
-            acc[41] += (double)v17_3_0;
-            acc[42] += (double)v18_1_0;
-            acc[43] += (double)v18_2_0;
-            acc[44] += (double)v18_3_0;
-            acc[45] += (double)v19_1_0;
-            acc[46] += (double)v19_2_0;
-            acc[47] += (double)v19_3_0;
+            if constexpr (sizeof(VT) == 8) {
+                acc[0] = fma(QCx, v4_0_0, fma(WQx, v4_0_1, fma(2.0 * oo2ze, v1_0_1, acc[0])));
+                acc[1] = fma(QCy, v4_0_0, fma(WQy, v4_0_1, acc[1]));
+                acc[2] = fma(QCz, v4_0_0, fma(WQz, v4_0_1, acc[2]));
+                acc[3] = fma(QCx, v5_0_0, fma(WQx, v5_0_1, fma(1.0 * oo2ze, v2_0_1, acc[3])));
+                acc[4] = fma(QCy, v5_0_0, fma(WQy, v5_0_1, fma(1.0 * oo2ze, v1_0_1, acc[4])));
+                acc[5] = fma(QCz, v5_0_0, fma(WQz, v5_0_1, acc[5]));
+                acc[6] = fma(QCx, v6_0_0, fma(WQx, v6_0_1, fma(1.0 * oo2ze, v3_0_1, acc[6])));
+                acc[7] = fma(QCy, v6_0_0, fma(WQy, v6_0_1, acc[7]));
+                acc[8] = fma(QCz, v6_0_0, fma(WQz, v6_0_1, fma(1.0 * oo2ze, v1_0_1, acc[8])));
+                acc[9] = fma(QCx, v7_0_0, fma(WQx, v7_0_1, acc[9]));
+                acc[10] = fma(QCy, v7_0_0, fma(WQy, v7_0_1, fma(2.0 * oo2ze, v2_0_1, acc[10])));
+                acc[11] = fma(QCz, v7_0_0, fma(WQz, v7_0_1, acc[11]));
+                acc[12] = fma(QCx, v8_0_0, fma(WQx, v8_0_1, acc[12]));
+                acc[13] = fma(QCy, v8_0_0, fma(WQy, v8_0_1, fma(1.0 * oo2ze, v3_0_1, acc[13])));
+                acc[14] = fma(QCz, v8_0_0, fma(WQz, v8_0_1, fma(1.0 * oo2ze, v2_0_1, acc[14])));
+                acc[15] = fma(QCx, v9_0_0, fma(WQx, v9_0_1, acc[15]));
+                acc[16] = fma(QCy, v9_0_0, fma(WQy, v9_0_1, acc[16]));
+                acc[17] = fma(QCz, v9_0_0, fma(WQz, v9_0_1, fma(2.0 * oo2ze, v3_0_1, acc[17])));
+                acc[18] = fma(QCx, v10_0_0, fma(WQx, v10_0_1, fma(3.0 * oo2ze, v4_0_1, acc[18])));
+                acc[19] = fma(QCy, v10_0_0, fma(WQy, v10_0_1, acc[19]));
+                acc[20] = fma(QCz, v10_0_0, fma(WQz, v10_0_1, acc[20]));
+                acc[21] = fma(QCx, v11_0_0, fma(WQx, v11_0_1, fma(2.0 * oo2ze, v5_0_1, acc[21])));
+                acc[22] = fma(QCy, v11_0_0, fma(WQy, v11_0_1, fma(1.0 * oo2ze, v4_0_1, acc[22])));
+                acc[23] = fma(QCz, v11_0_0, fma(WQz, v11_0_1, acc[23]));
+                acc[24] = fma(QCx, v12_0_0, fma(WQx, v12_0_1, fma(2.0 * oo2ze, v6_0_1, acc[24])));
+                acc[25] = fma(QCy, v12_0_0, fma(WQy, v12_0_1, acc[25]));
+                acc[26] = fma(QCz, v12_0_0, fma(WQz, v12_0_1, fma(1.0 * oo2ze, v4_0_1, acc[26])));
+                acc[27] = fma(QCx, v13_0_0, fma(WQx, v13_0_1, fma(1.0 * oo2ze, v7_0_1, acc[27])));
+                acc[28] = fma(QCy, v13_0_0, fma(WQy, v13_0_1, fma(2.0 * oo2ze, v5_0_1, acc[28])));
+                acc[29] = fma(QCz, v13_0_0, fma(WQz, v13_0_1, acc[29]));
+                acc[30] = fma(QCx, v14_0_0, fma(WQx, v14_0_1, fma(1.0 * oo2ze, v9_0_1, acc[30])));
+                acc[31] = fma(QCy, v14_0_0, fma(WQy, v14_0_1, acc[31]));
+                acc[32] = fma(QCz, v14_0_0, fma(WQz, v14_0_1, fma(2.0 * oo2ze, v6_0_1, acc[32])));
+                acc[33] = fma(QCx, v15_0_0, fma(WQx, v15_0_1, fma(1.0 * oo2ze, v8_0_1, acc[33])));
+                acc[34] = fma(QCy, v15_0_0, fma(WQy, v15_0_1, fma(1.0 * oo2ze, v6_0_1, acc[34])));
+                acc[35] = fma(QCz, v15_0_0, fma(WQz, v15_0_1, fma(1.0 * oo2ze, v5_0_1, acc[35])));
+                acc[36] = fma(QCx, v16_0_0, fma(WQx, v16_0_1, acc[36]));
+                acc[37] = fma(QCy, v16_0_0, fma(WQy, v16_0_1, fma(3.0 * oo2ze, v7_0_1, acc[37])));
+                acc[38] = fma(QCz, v16_0_0, fma(WQz, v16_0_1, acc[38]));
+                acc[39] = fma(QCx, v17_0_0, fma(WQx, v17_0_1, acc[39]));
+                acc[40] = fma(QCy, v17_0_0, fma(WQy, v17_0_1, fma(2.0 * oo2ze, v8_0_1, acc[40])));
+                acc[41] = fma(QCz, v17_0_0, fma(WQz, v17_0_1, fma(1.0 * oo2ze, v7_0_1, acc[41])));
+                acc[42] = fma(QCx, v18_0_0, fma(WQx, v18_0_1, acc[42]));
+                acc[43] = fma(QCy, v18_0_0, fma(WQy, v18_0_1, fma(1.0 * oo2ze, v9_0_1, acc[43])));
+                acc[44] = fma(QCz, v18_0_0, fma(WQz, v18_0_1, fma(2.0 * oo2ze, v8_0_1, acc[44])));
+                acc[45] = fma(QCx, v19_0_0, fma(WQx, v19_0_1, acc[45]));
+                acc[46] = fma(QCy, v19_0_0, fma(WQy, v19_0_1, acc[46]));
+                acc[47] = fma(QCz, v19_0_0, fma(WQz, v19_0_1, fma(3.0 * oo2ze, v9_0_1, acc[47])));
+            } else {
+                const VT v4_1_0 = QCx * v4_0_0 + WQx * v4_0_1 + (VT)2.0 * oo2ze * v1_0_1;
+                acc[0] += (double)v4_1_0;
+                const VT v4_2_0 = QCy * v4_0_0 + WQy * v4_0_1;
+                acc[1] += (double)v4_2_0;
+                const VT v4_3_0 = QCz * v4_0_0 + WQz * v4_0_1;
+                acc[2] += (double)v4_3_0;
+                const VT v5_1_0 = QCx * v5_0_0 + WQx * v5_0_1 + (VT)1.0 * oo2ze * v2_0_1;
+                acc[3] += (double)v5_1_0;
+                const VT v5_2_0 = QCy * v5_0_0 + WQy * v5_0_1 + (VT)1.0 * oo2ze * v1_0_1;
+                acc[4] += (double)v5_2_0;
+                const VT v5_3_0 = QCz * v5_0_0 + WQz * v5_0_1;
+                acc[5] += (double)v5_3_0;
+                const VT v6_1_0 = QCx * v6_0_0 + WQx * v6_0_1 + (VT)1.0 * oo2ze * v3_0_1;
+                acc[6] += (double)v6_1_0;
+                const VT v6_2_0 = QCy * v6_0_0 + WQy * v6_0_1;
+                acc[7] += (double)v6_2_0;
+                const VT v6_3_0 = QCz * v6_0_0 + WQz * v6_0_1 + (VT)1.0 * oo2ze * v1_0_1;
+                acc[8] += (double)v6_3_0;
+                const VT v7_1_0 = QCx * v7_0_0 + WQx * v7_0_1;
+                acc[9] += (double)v7_1_0;
+                const VT v7_2_0 = QCy * v7_0_0 + WQy * v7_0_1 + (VT)2.0 * oo2ze * v2_0_1;
+                acc[10] += (double)v7_2_0;
+                const VT v7_3_0 = QCz * v7_0_0 + WQz * v7_0_1;
+                acc[11] += (double)v7_3_0;
+                const VT v8_1_0 = QCx * v8_0_0 + WQx * v8_0_1;
+                acc[12] += (double)v8_1_0;
+                const VT v8_2_0 = QCy * v8_0_0 + WQy * v8_0_1 + (VT)1.0 * oo2ze * v3_0_1;
+                acc[13] += (double)v8_2_0;
+                const VT v8_3_0 = QCz * v8_0_0 + WQz * v8_0_1 + (VT)1.0 * oo2ze * v2_0_1;
+                acc[14] += (double)v8_3_0;
+                const VT v9_1_0 = QCx * v9_0_0 + WQx * v9_0_1;
+                acc[15] += (double)v9_1_0;
+                const VT v9_2_0 = QCy * v9_0_0 + WQy * v9_0_1;
+                acc[16] += (double)v9_2_0;
+                const VT v9_3_0 = QCz * v9_0_0 + WQz * v9_0_1 + (VT)2.0 * oo2ze * v3_0_1;
+                acc[17] += (double)v9_3_0;
+                const VT v10_1_0 = QCx * v10_0_0 + WQx * v10_0_1 + (VT)3.0 * oo2ze * v4_0_1;
+                acc[18] += (double)v10_1_0;
+                const VT v10_2_0 = QCy * v10_0_0 + WQy * v10_0_1;
+                acc[19] += (double)v10_2_0;
+                const VT v10_3_0 = QCz * v10_0_0 + WQz * v10_0_1;
+                acc[20] += (double)v10_3_0;
+                const VT v11_1_0 = QCx * v11_0_0 + WQx * v11_0_1 + (VT)2.0 * oo2ze * v5_0_1;
+                acc[21] += (double)v11_1_0;
+                const VT v11_2_0 = QCy * v11_0_0 + WQy * v11_0_1 + (VT)1.0 * oo2ze * v4_0_1;
+                acc[22] += (double)v11_2_0;
+                const VT v11_3_0 = QCz * v11_0_0 + WQz * v11_0_1;
+                acc[23] += (double)v11_3_0;
+                const VT v12_1_0 = QCx * v12_0_0 + WQx * v12_0_1 + (VT)2.0 * oo2ze * v6_0_1;
+                acc[24] += (double)v12_1_0;
+                const VT v12_2_0 = QCy * v12_0_0 + WQy * v12_0_1;
+                acc[25] += (double)v12_2_0;
+                const VT v12_3_0 = QCz * v12_0_0 + WQz * v12_0_1 + (VT)1.0 * oo2ze * v4_0_1;
+                acc[26] += (double)v12_3_0;
+                const VT v13_1_0 = QCx * v13_0_0 + WQx * v13_0_1 + (VT)1.0 * oo2ze * v7_0_1;
+                acc[27] += (double)v13_1_0;
+                const VT v13_2_0 = QCy * v13_0_0 + WQy * v13_0_1 + (VT)2.0 * oo2ze * v5_0_1;
+                acc[28] += (double)v13_2_0;
+                const VT v13_3_0 = QCz * v13_0_0 + WQz * v13_0_1;
+                acc[29] += (double)v13_3_0;
+                const VT v14_1_0 = QCx * v14_0_0 + WQx * v14_0_1 + (VT)1.0 * oo2ze * v9_0_1;
+                acc[30] += (double)v14_1_0;
+                const VT v14_2_0 = QCy * v14_0_0 + WQy * v14_0_1;
+                acc[31] += (double)v14_2_0;
+                const VT v14_3_0 = QCz * v14_0_0 + WQz * v14_0_1 + (VT)2.0 * oo2ze * v6_0_1;
+                acc[32] += (double)v14_3_0;
+                const VT v15_1_0 = QCx * v15_0_0 + WQx * v15_0_1 + (VT)1.0 * oo2ze * v8_0_1;
+                acc[33] += (double)v15_1_0;
+                const VT v15_2_0 = QCy * v15_0_0 + WQy * v15_0_1 + (VT)1.0 * oo2ze * v6_0_1;
+                acc[34] += (double)v15_2_0;
+                const VT v15_3_0 = QCz * v15_0_0 + WQz * v15_0_1 + (VT)1.0 * oo2ze * v5_0_1;
+                acc[35] += (double)v15_3_0;
+                const VT v16_1_0 = QCx * v16_0_0 + WQx * v16_0_1;
+                acc[36] += (double)v16_1_0;
+                const VT v16_2_0 = QCy * v16_0_0 + WQy * v16_0_1 + (VT)3.0 * oo2ze * v7_0_1;
+                acc[37] += (double)v16_2_0;
+                const VT v16_3_0 = QCz * v16_0_0 + WQz * v16_0_1;
+                acc[38] += (double)v16_3_0;
+                const VT v17_1_0 = QCx * v17_0_0 + WQx * v17_0_1;
+                acc[39] += (double)v17_1_0;
+                const VT v17_2_0 = QCy * v17_0_0 + WQy * v17_0_1 + (VT)2.0 * oo2ze * v8_0_1;
+                acc[40] += (double)v17_2_0;
+                const VT v17_3_0 = QCz * v17_0_0 + WQz * v17_0_1 + (VT)1.0 * oo2ze * v7_0_1;
+                acc[41] += (double)v17_3_0;
+                const VT v18_1_0 = QCx * v18_0_0 + WQx * v18_0_1;
+                acc[42] += (double)v18_1_0;
+                const VT v18_2_0 = QCy * v18_0_0 + WQy * v18_0_1 + (VT)1.0 * oo2ze * v9_0_1;
+                acc[43] += (double)v18_2_0;
+                const VT v18_3_0 = QCz * v18_0_0 + WQz * v18_0_1 + (VT)2.0 * oo2ze * v8_0_1;
+                acc[44] += (double)v18_3_0;
+                const VT v19_1_0 = QCx * v19_0_0 + WQx * v19_0_1;
+                acc[45] += (double)v19_1_0;
+                const VT v19_2_0 = QCy * v19_0_0 + WQy * v19_0_1;
+                acc[46] += (double)v19_2_0;
+                const VT v19_3_0 = QCz * v19_0_0 + WQz * v19_0_1 + (VT)3.0 * oo2ze * v9_0_1;
+                acc[47] += (double)v19_3_0;
+            }
         }
     }
 }

@@ -25,13 +25,13 @@ __device__ __forceinline__ void vrr_dpss(const PairTab &P, const BoysTab &B, int
             const double r = rsqrt(bra.zeta + ket.zeta);
             const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
-            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[4];
             boys_fm<3>(T, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
-            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
             const VT WQx = (VT)(zz * PQx), WQy = (VT)(zz * PQy), WQz = (VT)(zz * PQz);
             const VT oo2z = (VT)bra.oo2z, oo2e = (VT)ket.oo2z, oo2ze = (VT)(0.5 * r2);
@@ -64,32 +64,22 @@ __device__ __forceinline__ void vrr_dpss(const PairTab &P, const BoysTab &B, int
             const VT v8_0_1 = PAy * v3_0_1 + WPy * v3_0_2;
             const VT v9_0_0 = PAz * v3_0_0 + WPz * v3_0_1 + (VT)1.0 * oo2z * (v0_0_0 - rho_z * v0_0_1);
             const VT v9_0_1 = PAz * v3_0_1 + WPz * v3_0_2 + (VT)1.0 * oo2z * (v0_0_1 - rho_z * v0_0_2);
-            const VT v10_0_0 = PAx * v4_0_0 + WPx * v4_0_1 + (VT)2.0 * oo2z * (v1_0_0 - rho_z * v1_0_1);
-            const VT v11_0_0 = PAx * v5_0_0 + WPx * v5_0_1 + (VT)1.0 * oo2z * (v2_0_0 - rho_z * v2_0_1);
-            const VT v12_0_0 = PAx * v6_0_0 + WPx * v6_0_1 + (VT)1.0 * oo2z * (v3_0_0 - rho_z * v3_0_1);
-            const VT v13_0_0 = PAy * v5_0_0 + WPy * v5_0_1 + (VT)1.0 * oo2z * (v1_0_0 - rho_z * v1_0_1);
-            const VT v14_0_0 = PAz * v6_0_0 + WPz * v6_0_1 + (VT)1.0 * oo2z * (v1_0_0 - rho_z * v1_0_1);
-            const VT v15_0_0 = PAx * v8_0_0 + WPx * v8_0_1;
-            const VT v16_0_0 = PAy * v7_0_0 + WPy * v7_0_1 + (VT)2.0 * oo2z * (v2_0_0 - rho_z * v2_0_1);
-            const VT v17_0_0 = PAy * v8_0_0 + WPy * v8_0_1 + (VT)1.0 * oo2z * (v3_0_0 - rho_z * v3_0_1);
-            const VT v18_0_0 = PAz * v8_0_0 + WPz * v8_0_1 + (VT)1.0 * oo2z * (v2_0_0 - rho_z * v2_0_1);
-            const VT v19_0_0 = PAz * v9_0_0 + WPz * v9_0_1 + (VT)2.0 * oo2z * (v3_0_0 - rho_z * v3_0_1);
             acc[0] += (double)v4_0_0;
             acc[1] += (double)v5_0_0;
             acc[2] += (double)v6_0_0;
             acc[3] += (double)v7_0_0;
             acc[4] += (double)v8_0_0;
             acc[5] += (double)v9_0_0;
-            acc[6] += (double)v10_0_0;
-            acc[7] += (double)v11_0_0;
-            acc[8] += (double)v12_0_0;
-            acc[9] += (double)v13_0_0;
-            acc[10] += (double)v14_0_0;
-            acc[11] += (double)v15_0_0;
-            acc[12] += (double)v16_0_0;
-            acc[13] += (double)v17_0_0;
-            acc[14] += (double)v18_0_0;
-            acc[15] += (double)v19_0_0;
+            acc[6] = fma(PAx, v4_0_0, fma(WPx, v4_0_1, fma(2.0 * oo2z, (v1_0_0 - rho_z * v1_0_1), acc[6])));
+            acc[7] = fma(PAx, v5_0_0, fma(WPx, v5_0_1, fma(1.0 * oo2z, (v2_0_0 - rho_z * v2_0_1), acc[7])));
+            acc[8] = fma(PAx, v6_0_0, fma(WPx, v6_0_1, fma(1.0 * oo2z, (v3_0_0 - rho_z * v3_0_1), acc[8])));
+            acc[9] = fma(PAy, v5_0_0, fma(WPy, v5_0_1, fma(1.0 * oo2z, (v1_0_0 - rho_z * v1_0_1), acc[9])));
+            acc[10] = fma(PAz, v6_0_0, fma(WPz, v6_0_1, fma(1.0 * oo2z, (v1_0_0 - rho_z * v1_0_1), acc[10])));
+            acc[11] = fma(PAx, v8_0_0, fma(WPx, v8_0_1, acc[11]));
+            acc[12] = fma(PAy, v7_0_0, fma(WPy, v7_0_1, fma(2.0 * oo2z, (v2_0_0 - rho_z * v2_0_1), acc[12])));
+            acc[13] = fma(PAy, v8_0_0, fma(WPy, v8_0_1, fma(1.0 * oo2z, (v3_0_0 - rho_z * v3_0_1), acc[13])));
+            acc[14] = fma(PAz, v8_0_0, fma(WPz, v8_0_1, fma(1.0 * oo2z, (v2_0_0 - rho_z * v2_0_1), acc[14])));
+            acc[15] = fma(PAz, v9_0_0, fma(WPz, v9_0_1, fma(2.0 * oo2z, (v3_0_0 - rho_z * v3_0_1), acc[15])));
         }
     }
 }

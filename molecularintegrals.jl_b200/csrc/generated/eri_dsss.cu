@@ -25,13 +25,13 @@ __device__ __forceinline__ void vrr_dsss(const PairTab &P, const BoysTab &B, int
             const double r = rsqrt(bra.zeta + ket.zeta);
             const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
-            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[3];
             boys_fm<2>(T, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
-            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
             const VT WQx = (VT)(zz * PQx), WQy = (VT)(zz * PQy), WQz = (VT)(zz * PQz);
             const VT oo2z = (VT)bra.oo2z, oo2e = (VT)ket.oo2z, oo2ze = (VT)(0.5 * r2);
@@ -48,18 +48,12 @@ __device__ __forceinline__ void vrr_dsss(const PairTab &P, const BoysTab &B, int
             const VT v2_0_1 = PAy * v0_0_1 + WPy * v0_0_2;
             const VT v3_0_0 = PAz * v0_0_0 + WPz * v0_0_1;
             const VT v3_0_1 = PAz * v0_0_1 + WPz * v0_0_2;
-            const VT v4_0_0 = PAx * v1_0_0 + WPx * v1_0_1 + (VT)1.0 * oo2z * (v0_0_0 - rho_z * v0_0_1);
-            const VT v5_0_0 = PAx * v2_0_0 + WPx * v2_0_1;
-            const VT v6_0_0 = PAx * v3_0_0 + WPx * v3_0_1;
-            const VT v7_0_0 = PAy * v2_0_0 + WPy * v2_0_1 + (VT)1.0 * oo2z * (v0_0_0 - rho_z * v0_0_1);
-            const VT v8_0_0 = PAy * v3_0_0 + WPy * v3_0_1;
-            const VT v9_0_0 = PAz * v3_0_0 + WPz * v3_0_1 + (VT)1.0 * oo2z * (v0_0_0 - rho_z * v0_0_1);
-            acc[0] += (double)v4_0_0;
-            acc[1] += (double)v5_0_0;
-            acc[2] += (double)v6_0_0;
-            acc[3] += (double)v7_0_0;
-            acc[4] += (double)v8_0_0;
-            acc[5] += (double)v9_0_0;
+            acc[0] = fma(PAx, v1_0_0, fma(WPx, v1_0_1, fma(1.0 * oo2z, (v0_0_0 - rho_z * v0_0_1), acc[0])));
+            acc[1] = fma(PAx, v2_0_0, fma(WPx, v2_0_1, acc[1]));
+            acc[2] = fma(PAx, v3_0_0, fma(WPx, v3_0_1, acc[2]));
+            acc[3] = fma(PAy, v2_0_0, fma(WPy, v2_0_1, fma(1.0 * oo2z, (v0_0_0 - rho_z * v0_0_1), acc[3])));
+            acc[4] = fma(PAy, v3_0_0, fma(WPy, v3_0_1, acc[4]));
+            acc[5] = fma(PAz, v3_0_0, fma(WPz, v3_0_1, fma(1.0 * oo2z, (v0_0_0 - rho_z * v0_0_1), acc[5])));
         }
     }
 }

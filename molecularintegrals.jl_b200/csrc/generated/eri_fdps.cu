@@ -25,13 +25,13 @@ __device__ __forceinline__ void vrr_fdps(const PairTab &P, const BoysTab &B, int
             const double r = rsqrt(bra.zeta + ket.zeta);
             const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
-            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[7];
             boys_fm<6>(T, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
-            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
             const VT WQx = (VT)(zz * PQx), WQy = (VT)(zz * PQy), WQz = (VT)(zz * PQz);
             const VT oo2z = (VT)bra.oo2z, oo2e = (VT)ket.oo2z, oo2ze = (VT)(0.5 * r2);
@@ -221,282 +221,423 @@ __device__ __forceinline__ void vrr_fdps(const PairTab &P, const BoysTab &B, int
             const VT v54_0_1 = PAz * v33_0_1 + WPz * v33_0_2 + (VT)3.0 * oo2z * (v18_0_1 - rho_z * v18_0_2);
             const VT v55_0_0 = PAz * v34_0_0 + WPz * v34_0_1 + (VT)4.0 * oo2z * (v19_0_0 - rho_z * v19_0_1);
             const VT v55_0_1 = PAz * v34_0_1 + WPz * v34_0_2 + (VT)4.0 * oo2z * (v19_0_1 - rho_z * v19_0_2);
-            const VT v10_1_0 = QCx * v10_0_0 + WQx * v10_0_1 + (VT)3.0 * oo2ze * v4_0_1;
-            const VT v11_1_0 = QCx * v11_0_0 + WQx * v11_0_1 + (VT)2.0 * oo2ze * v5_0_1;
-            const VT v12_1_0 = QCx * v12_0_0 + WQx * v12_0_1 + (VT)2.0 * oo2ze * v6_0_1;
-            const VT v13_1_0 = QCx * v13_0_0 + WQx * v13_0_1 + (VT)1.0 * oo2ze * v7_0_1;
-            const VT v14_1_0 = QCx * v14_0_0 + WQx * v14_0_1 + (VT)1.0 * oo2ze * v9_0_1;
-            const VT v15_1_0 = QCx * v15_0_0 + WQx * v15_0_1 + (VT)1.0 * oo2ze * v8_0_1;
-            const VT v16_1_0 = QCx * v16_0_0 + WQx * v16_0_1;
-            const VT v17_1_0 = QCx * v17_0_0 + WQx * v17_0_1;
-            const VT v18_1_0 = QCx * v18_0_0 + WQx * v18_0_1;
-            const VT v19_1_0 = QCx * v19_0_0 + WQx * v19_0_1;
-            const VT v20_1_0 = QCx * v20_0_0 + WQx * v20_0_1 + (VT)4.0 * oo2ze * v10_0_1;
-            const VT v21_1_0 = QCx * v21_0_0 + WQx * v21_0_1 + (VT)3.0 * oo2ze * v11_0_1;
-            const VT v22_1_0 = QCx * v22_0_0 + WQx * v22_0_1 + (VT)3.0 * oo2ze * v12_0_1;
-            const VT v23_1_0 = QCx * v23_0_0 + WQx * v23_0_1 + (VT)2.0 * oo2ze * v13_0_1;
-            const VT v24_1_0 = QCx * v24_0_0 + WQx * v24_0_1 + (VT)2.0 * oo2ze * v15_0_1;
-            const VT v25_1_0 = QCx * v25_0_0 + WQx * v25_0_1 + (VT)2.0 * oo2ze * v14_0_1;
-            const VT v26_1_0 = QCx * v26_0_0 + WQx * v26_0_1 + (VT)1.0 * oo2ze * v16_0_1;
-            const VT v27_1_0 = QCx * v27_0_0 + WQx * v27_0_1 + (VT)1.0 * oo2ze * v17_0_1;
-            const VT v28_1_0 = QCx * v28_0_0 + WQx * v28_0_1 + (VT)1.0 * oo2ze * v18_0_1;
-            const VT v29_1_0 = QCx * v29_0_0 + WQx * v29_0_1 + (VT)1.0 * oo2ze * v19_0_1;
-            const VT v30_1_0 = QCx * v30_0_0 + WQx * v30_0_1;
-            const VT v31_1_0 = QCx * v31_0_0 + WQx * v31_0_1;
-            const VT v32_1_0 = QCx * v32_0_0 + WQx * v32_0_1;
-            const VT v33_1_0 = QCx * v33_0_0 + WQx * v33_0_1;
-            const VT v34_1_0 = QCx * v34_0_0 + WQx * v34_0_1;
-            const VT v35_1_0 = QCx * v35_0_0 + WQx * v35_0_1 + (VT)5.0 * oo2ze * v20_0_1;
-            const VT v36_1_0 = QCx * v36_0_0 + WQx * v36_0_1 + (VT)4.0 * oo2ze * v21_0_1;
-            const VT v37_1_0 = QCx * v37_0_0 + WQx * v37_0_1 + (VT)4.0 * oo2ze * v22_0_1;
-            const VT v38_1_0 = QCx * v38_0_0 + WQx * v38_0_1 + (VT)3.0 * oo2ze * v23_0_1;
-            const VT v39_1_0 = QCx * v39_0_0 + WQx * v39_0_1 + (VT)3.0 * oo2ze * v24_0_1;
-            const VT v40_1_0 = QCx * v40_0_0 + WQx * v40_0_1 + (VT)3.0 * oo2ze * v25_0_1;
-            const VT v41_1_0 = QCx * v41_0_0 + WQx * v41_0_1 + (VT)2.0 * oo2ze * v26_0_1;
-            const VT v42_1_0 = QCx * v42_0_0 + WQx * v42_0_1 + (VT)2.0 * oo2ze * v27_0_1;
-            const VT v43_1_0 = QCx * v43_0_0 + WQx * v43_0_1 + (VT)2.0 * oo2ze * v28_0_1;
-            const VT v44_1_0 = QCx * v44_0_0 + WQx * v44_0_1 + (VT)2.0 * oo2ze * v29_0_1;
-            const VT v45_1_0 = QCx * v45_0_0 + WQx * v45_0_1 + (VT)1.0 * oo2ze * v30_0_1;
-            const VT v46_1_0 = QCx * v46_0_0 + WQx * v46_0_1 + (VT)1.0 * oo2ze * v31_0_1;
-            const VT v47_1_0 = QCx * v47_0_0 + WQx * v47_0_1 + (VT)1.0 * oo2ze * v32_0_1;
-            const VT v48_1_0 = QCx * v48_0_0 + WQx * v48_0_1 + (VT)1.0 * oo2ze * v33_0_1;
-            const VT v49_1_0 = QCx * v49_0_0 + WQx * v49_0_1 + (VT)1.0 * oo2ze * v34_0_1;
-            const VT v50_1_0 = QCx * v50_0_0 + WQx * v50_0_1;
-            const VT v51_1_0 = QCx * v51_0_0 + WQx * v51_0_1;
-            const VT v52_1_0 = QCx * v52_0_0 + WQx * v52_0_1;
-            const VT v53_1_0 = QCx * v53_0_0 + WQx * v53_0_1;
-            const VT v54_1_0 = QCx * v54_0_0 + WQx * v54_0_1;
-            const VT v55_1_0 = QCx * v55_0_0 + WQx * v55_0_1;
-            const VT v10_2_0 = QCy * v10_0_0 + WQy * v10_0_1;
-            const VT v11_2_0 = QCy * v11_0_0 + WQy * v11_0_1 + (VT)1.0 * oo2ze * v4_0_1;
-            const VT v12_2_0 = QCy * v12_0_0 + WQy * v12_0_1;
-            const VT v13_2_0 = QCy * v13_0_0 + WQy * v13_0_1 + (VT)2.0 * oo2ze * v5_0_1;
-            const VT v14_2_0 = QCy * v14_0_0 + WQy * v14_0_1;
-            const VT v15_2_0 = QCy * v15_0_0 + WQy * v15_0_1 + (VT)1.0 * oo2ze * v6_0_1;
-            const VT v16_2_0 = QCy * v16_0_0 + WQy * v16_0_1 + (VT)3.0 * oo2ze * v7_0_1;
-            const VT v17_2_0 = QCy * v17_0_0 + WQy * v17_0_1 + (VT)2.0 * oo2ze * v8_0_1;
-            const VT v18_2_0 = QCy * v18_0_0 + WQy * v18_0_1 + (VT)1.0 * oo2ze * v9_0_1;
-            const VT v19_2_0 = QCy * v19_0_0 + WQy * v19_0_1;
-            const VT v20_2_0 = QCy * v20_0_0 + WQy * v20_0_1;
-            const VT v21_2_0 = QCy * v21_0_0 + WQy * v21_0_1 + (VT)1.0 * oo2ze * v10_0_1;
-            const VT v22_2_0 = QCy * v22_0_0 + WQy * v22_0_1;
-            const VT v23_2_0 = QCy * v23_0_0 + WQy * v23_0_1 + (VT)2.0 * oo2ze * v11_0_1;
-            const VT v24_2_0 = QCy * v24_0_0 + WQy * v24_0_1 + (VT)1.0 * oo2ze * v12_0_1;
-            const VT v25_2_0 = QCy * v25_0_0 + WQy * v25_0_1;
-            const VT v26_2_0 = QCy * v26_0_0 + WQy * v26_0_1 + (VT)3.0 * oo2ze * v13_0_1;
-            const VT v27_2_0 = QCy * v27_0_0 + WQy * v27_0_1 + (VT)2.0 * oo2ze * v15_0_1;
-            const VT v28_2_0 = QCy * v28_0_0 + WQy * v28_0_1 + (VT)1.0 * oo2ze * v14_0_1;
-            const VT v29_2_0 = QCy * v29_0_0 + WQy * v29_0_1;
-            const VT v30_2_0 = QCy * v30_0_0 + WQy * v30_0_1 + (VT)4.0 * oo2ze * v16_0_1;
-            const VT v31_2_0 = QCy * v31_0_0 + WQy * v31_0_1 + (VT)3.0 * oo2ze * v17_0_1;
-            const VT v32_2_0 = QCy * v32_0_0 + WQy * v32_0_1 + (VT)2.0 * oo2ze * v18_0_1;
-            const VT v33_2_0 = QCy * v33_0_0 + WQy * v33_0_1 + (VT)1.0 * oo2ze * v19_0_1;
-            const VT v34_2_0 = QCy * v34_0_0 + WQy * v34_0_1;
-            const VT v35_2_0 = QCy * v35_0_0 + WQy * v35_0_1;
-            const VT v36_2_0 = QCy * v36_0_0 + WQy * v36_0_1 + (VT)1.0 * oo2ze * v20_0_1;
-            const VT v37_2_0 = QCy * v37_0_0 + WQy * v37_0_1;
-            const VT v38_2_0 = QCy * v38_0_0 + WQy * v38_0_1 + (VT)2.0 * oo2ze * v21_0_1;
-            const VT v39_2_0 = QCy * v39_0_0 + WQy * v39_0_1 + (VT)1.0 * oo2ze * v22_0_1;
-            const VT v40_2_0 = QCy * v40_0_0 + WQy * v40_0_1;
-            const VT v41_2_0 = QCy * v41_0_0 + WQy * v41_0_1 + (VT)3.0 * oo2ze * v23_0_1;
-            const VT v42_2_0 = QCy * v42_0_0 + WQy * v42_0_1 + (VT)2.0 * oo2ze * v24_0_1;
-            const VT v43_2_0 = QCy * v43_0_0 + WQy * v43_0_1 + (VT)1.0 * oo2ze * v25_0_1;
-            const VT v44_2_0 = QCy * v44_0_0 + WQy * v44_0_1;
-            const VT v45_2_0 = QCy * v45_0_0 + WQy * v45_0_1 + (VT)4.0 * oo2ze * v26_0_1;
-            const VT v46_2_0 = QCy * v46_0_0 + WQy * v46_0_1 + (VT)3.0 * oo2ze * v27_0_1;
-            const VT v47_2_0 = QCy * v47_0_0 + WQy * v47_0_1 + (VT)2.0 * oo2ze * v28_0_1;
-            const VT v48_2_0 = QCy * v48_0_0 + WQy * v48_0_1 + (VT)1.0 * oo2ze * v29_0_1;
-            const VT v49_2_0 = QCy * v49_0_0 + WQy * v49_0_1;
-            const VT v50_2_0 = QCy * v50_0_0 + WQy * v50_0_1 + (VT)5.0 * oo2ze * v30_0_1;
-            const VT v51_2_0 = QCy * v51_0_0 + WQy * v51_0_1 + (VT)4.0 * oo2ze * v31_0_1;
-            const VT v52_2_0 = QCy * v52_0_0 + WQy * v52_0_1 + (VT)3.0 * oo2ze * v32_0_1;
-            const VT v53_2_0 = QCy * v53_0_0 + WQy * v53_0_1 + (VT)2.0 * oo2ze * v33_0_1;
-            const VT v54_2_0 = QCy * v54_0_0 + WQy * v54_0_1 + (VT)1.0 * oo2ze * v34_0_1;
-            const VT v55_2_0 = QCy * v55_0_0 + WQy * v55_0_1;
-            const VT v10_3_0 = QCz * v10_0_0 + WQz * v10_0_1;
-            const VT v11_3_0 = QCz * v11_0_0 + WQz * v11_0_1;
-            const VT v12_3_0 = QCz * v12_0_0 + WQz * v12_0_1 + (VT)1.0 * oo2ze * v4_0_1;
-            const VT v13_3_0 = QCz * v13_0_0 + WQz * v13_0_1;
-            const VT v14_3_0 = QCz * v14_0_0 + WQz * v14_0_1 + (VT)2.0 * oo2ze * v6_0_1;
-            const VT v15_3_0 = QCz * v15_0_0 + WQz * v15_0_1 + (VT)1.0 * oo2ze * v5_0_1;
-            const VT v16_3_0 = QCz * v16_0_0 + WQz * v16_0_1;
-            const VT v17_3_0 = QCz * v17_0_0 + WQz * v17_0_1 + (VT)1.0 * oo2ze * v7_0_1;
-            const VT v18_3_0 = QCz * v18_0_0 + WQz * v18_0_1 + (VT)2.0 * oo2ze * v8_0_1;
-            const VT v19_3_0 = QCz * v19_0_0 + WQz * v19_0_1 + (VT)3.0 * oo2ze * v9_0_1;
-            const VT v20_3_0 = QCz * v20_0_0 + WQz * v20_0_1;
-            const VT v21_3_0 = QCz * v21_0_0 + WQz * v21_0_1;
-            const VT v22_3_0 = QCz * v22_0_0 + WQz * v22_0_1 + (VT)1.0 * oo2ze * v10_0_1;
-            const VT v23_3_0 = QCz * v23_0_0 + WQz * v23_0_1;
-            const VT v24_3_0 = QCz * v24_0_0 + WQz * v24_0_1 + (VT)1.0 * oo2ze * v11_0_1;
-            const VT v25_3_0 = QCz * v25_0_0 + WQz * v25_0_1 + (VT)2.0 * oo2ze * v12_0_1;
-            const VT v26_3_0 = QCz * v26_0_0 + WQz * v26_0_1;
-            const VT v27_3_0 = QCz * v27_0_0 + WQz * v27_0_1 + (VT)1.0 * oo2ze * v13_0_1;
-            const VT v28_3_0 = QCz * v28_0_0 + WQz * v28_0_1 + (VT)2.0 * oo2ze * v15_0_1;
-            const VT v29_3_0 = QCz * v29_0_0 + WQz * v29_0_1 + (VT)3.0 * oo2ze * v14_0_1;
-            const VT v30_3_0 = QCz * v30_0_0 + WQz * v30_0_1;
-            const VT v31_3_0 = QCz * v31_0_0 + WQz * v31_0_1 + (VT)1.0 * oo2ze * v16_0_1;
-            const VT v32_3_0 = QCz * v32_0_0 + WQz * v32_0_1 + (VT)2.0 * oo2ze * v17_0_1;
-            const VT v33_3_0 = QCz * v33_0_0 + WQz * v33_0_1 + (VT)3.0 * oo2ze * v18_0_1;
-            const VT v34_3_0 = QCz * v34_0_0 + WQz * v34_0_1 + (VT)4.0 * oo2ze * v19_0_1;
-            const VT v35_3_0 = QCz * v35_0_0 + WQz * v35_0_1;
-            const VT v36_3_0 = QCz * v36_0_0 + WQz * v36_0_1;
-            const VT v37_3_0 = QCz * v37_0_0 + WQz * v37_0_1 + (VT)1.0 * oo2ze * v20_0_1;
-            const VT v38_3_0 = QCz * v38_0_0 + WQz * v38_0_1;
-            const VT v39_3_0 = QCz * v39_0_0 + WQz * v39_0_1 + (VT)1.0 * oo2ze * v21_0_1;
-            const VT v40_3_0 = QCz * v40_0_0 + WQz * v40_0_1 + (VT)2.0 * oo2ze * v22_0_1;
-            const VT v41_3_0 = QCz * v41_0_0 + WQz * v41_0_1;
-            const VT v42_3_0 = QCz * v42_0_0 + WQz * v42_0_1 + (VT)1.0 * oo2ze * v23_0_1;
-            const VT v43_3_0 = QCz * v43_0_0 + WQz * v43_0_1 + (VT)2.0 * oo2ze * v24_0_1;
-            const VT v44_3_0 = QCz * v44_0_0 + WQz * v44_0_1 + (VT)3.0 * oo2ze * v25_0_1;
-            const VT v45_3_0 = QCz * v45_0_0 + WQz * v45_0_1;
-            const VT v46_3_0 = QCz * v46_0_0 + WQz * v46_0_1 + (VT)1.0 * oo2ze * v26_0_1;
-            const VT v47_3_0 = QCz * v47_0_0 + WQz * v47_0_1 + (VT)2.0 * oo2ze * v27_0_1;
-            const VT v48_3_0 = QCz * v48_0_0 + WQz * v48_0_1 + (VT)3.0 * oo2ze * v28_0_1;
-            const VT v49_3_0 = QCz * v49_0_0 + WQz * v49_0_1 + (VT)4.0 * oo2ze * v29_0_1;
-            const VT v50_3_0 = QCz * v50_0_0 + WQz * v50_0_1;
-            const VT v51_3_0 = QCz * v51_0_0 + WQz * v51_0_1 + (VT)1.0 * oo2ze * v30_0_1;
-            const VT v52_3_0 = QCz * v52_0_0 + WQz * v52_0_1 + (VT)2.0 * oo2ze * v31_0_1;
-            const VT v53_3_0 = QCz * v53_0_0 + WQz * v53_0_1 + (VT)3.0 * oo2ze * v32_0_1;
-            const VT v54_3_0 = QCz * v54_0_0 + WQz * v54_0_1 + (VT)4.0 * oo2ze * v33_0_1;
-            const VT v55_3_0 = QCz * v55_0_0 + WQz * v55_0_1 + (VT)5.0 * oo2ze * v34_0_1;
-            acc[0] += (double)v10_1_0;
-            acc[1] += (double)v10_2_0;
-            acc[2] += (double)v10_3_0;
-            acc[3] += (double)v11_1_0;
-            acc[4] += (double)v11_2_0;
-            acc[5] += (double)v11_3_0;
-            acc[6] += (double)v12_1_0;
-            acc[7] += (double)v12_2_0;
-            acc[8] += (double)v12_3_0;
-            acc[9] += (double)v13_1_0;
-            acc[10] += (double)v13_2_0;
-            acc[11] += (double)v13_3_0;
-            acc[12] += (double)v14_1_0;
-            acc[13] += (double)v14_2_0;
-            acc[14] += (double)v14_3_0;
-            acc[15] += (double)v15_1_0;
-            acc[16] += (double)v15_2_0;
-            acc[17] += (double)v15_3_0;
-            acc[18] += (double)v16_1_0;
-            acc[19] += (double)v16_2_0;
-            acc[20] += (double)v16_3_0;
-            acc[21] += (double)v17_1_0;
-            acc[22] += (double)v17_2_0;
-            acc[23] += (double)v17_3_0;
-            acc[24] += (double)v18_1_0;
-            acc[25] += (double)v18_2_0;
-            acc[26] += (double)v18_3_0;
-            acc[27] += (double)v19_1_0;
-            acc[28] += (double)v19_2_0;
-            acc[29] += (double)v19_3_0;
-            acc[30] += (double)v20_1_0;
-            acc[31] += (double)v20_2_0;
-            acc[32] += (double)v20_3_0;
-            acc[33] += (double)v21_1_0;
-            acc[34] += (double)v21_2_0;
-            acc[35] += (double)v21_3_0;
-            acc[36] += (double)v22_1_0;
-            acc[37] += (double)v22_2_0;
-            acc[38] += (double)v22_3_0;
-            acc[39] += (double)v23_1_0;
-            acc[40] += (double)v23_2_0;
-            acc[41] += (double)v23_3_0;
-            acc[42] += (double)v24_1_0;
-            acc[43] += (double)v24_2_0;
-            acc[44] += (double)v24_3_0;
-            acc[45] += (double)v25_1_0;
-            acc[46] += (double)v25_2_0;
-            acc[47] += (double)v25_3_0;
-            acc[48] += (double)v26_1_0;
-            acc[49] += (double)v26_2_0;
-            acc[50] += (double)v26_3_0;
-            acc[51] += (double)v27_1_0;
-            acc[52] += (double)v27_2_0;
-            acc[53] += (double)v27_3_0;
-            acc[54] += (double)v28_1_0;
-            acc[55] += (double)v28_2_0;
-            acc[56] += (double)v28_3_0;
-            acc[57] += (double)v29_1_0;
-            acc[58] += (double)v29_2_0;
-            acc[59] += (double)v29_3_0;
-            acc[60] += (double)v30_1_0;
-            acc[61] += (double)v30_2_0;
-            acc[62] += (double)v30_3_0;
-            acc[63] += (double)v31_1_0;
-            acc[64] += (double)v31_2_0;
-            acc[65] += (double)v31_3_0;
-            acc[66] += (double)v32_1_0;
-            acc[67] += (double)v32_2_0;
-            acc[68] += (double)v32_3_0;
-            acc[69] += (double)v33_1_0;
-            acc[70] += (double)v33_2_0;
-            acc[71] += (double)v33_3_0;
-            acc[72] += (double)v34_1_0;
-            acc[73] += (double)v34_2_0;
-            acc[74] += (double)v34_3_0;
-            acc[75] += (double)v35_1_0;
-            acc[76] += (double)v35_2_0;
-            acc[77] += (double)v35_3_0;
-            acc[78] += (double)v36_1_0;
-            acc[79] += (double)v36_2_0;
-            acc[80] += (double)v36_3_0;
-            acc[81] += (double)v37_1_0;
-            acc[82] += (double)v37_2_0;
-            acc[83] += (double)v37_3_0;
-            acc[84] += (double)v38_1_0;
-            acc[85] += (double)v38_2_0;
-            acc[86] += (double)v38_3_0;
-            acc[87] += (double)v39_1_0;
-            acc[88] += (double)v39_2_0;
-            acc[89] += (double)v39_3_0;
-            acc[90] += (double)v40_1_0;
-            acc[91] += (double)v40_2_0;
-            acc[92] += (double)v40_3_0;
-            acc[93] += (double)v41_1_0;
-            acc[94] += (double)v41_2_0;
-            acc[95] += (double)v41_3_0;
-            acc[96] += (double)v42_1_0;
-            acc[97] += (double)v42_2_0;
-            acc[98] += (double)v42_3_0;
-            acc[99] += (double)v43_1_0;
-            acc[100] += (double)v43_2_0;
-            acc[101] += (double)v43_3_0;
-            acc[102] += (double)v44_1_0;
-            acc[103] += (double)v44_2_0;
-            acc[104] += (double)v44_3_0;
-            acc[105] += (double)v45_1_0;
-            acc[106] += (double)v45_2_0;
-            acc[107] += (double)v45_3_0;
-            acc[108] += (double)v46_1_0;
-            acc[109] += (double)v46_2_0;
-            acc[110] += (double)v46_3_0;
-            acc[111] += (double)v47_1_0;
-            acc[112] += (double)v47_2_0;
-            acc[113] += (double)v47_3_0;
-            acc[114] += (double)v48_1_0;
-            acc[115] += (double)v48_2_0;
-            acc[116] += (double)v48_3_0;
-            acc[117] += (double)v49_1_0;
-            acc[118] += (double)v49_2_0;
-            acc[119] += (double)v49_3_0;
-            acc[120] += (double)v50_1_0;
-            acc[121] += (double)v50_2_0;
-            acc[122] += (double)v50_3_0;
-            acc[123] += (double)v51_1_0;
-            acc[124] += (double)v51_2_0;
-            acc[125] += (double)v51_3_0;
-            acc[126] += (double)v52_1_0;
-            acc[127] += (double)v52_2_0;
-            acc[128] += (double)v52_3_0;
-            acc[129] += (double)v53_1_0;
-            acc[130] += (double)v53_2_0;
-            acc[131] += (double)v53_3_0;
-            acc[132] += (double)v54_1_0;
-            acc[133] += (double)v54_2_0;
-            acc[134] += (double)v54_3_0;
-            acc[135] += (double)v55_1_0;
-            acc[136] += (double)v55_2_0;
-            acc[137] += (double)v55_3_0;
+            if constexpr (sizeof(VT) == 8) {
+                acc[0] = fma(QCx, v10_0_0, fma(WQx, v10_0_1, fma(3.0 * oo2ze, v4_0_1, acc[0])));
+                acc[1] = fma(QCy, v10_0_0, fma(WQy, v10_0_1, acc[1]));
+                acc[2] = fma(QCz, v10_0_0, fma(WQz, v10_0_1, acc[2]));
+                acc[3] = fma(QCx, v11_0_0, fma(WQx, v11_0_1, fma(2.0 * oo2ze, v5_0_1, acc[3])));
+                acc[4] = fma(QCy, v11_0_0, fma(WQy, v11_0_1, fma(1.0 * oo2ze, v4_0_1, acc[4])));
+                acc[5] = fma(QCz, v11_0_0, fma(WQz, v11_0_1, acc[5]));
+                acc[6] = fma(QCx, v12_0_0, fma(WQx, v12_0_1, fma(2.0 * oo2ze, v6_0_1, acc[6])));
+                acc[7] = fma(QCy, v12_0_0, fma(WQy, v12_0_1, acc[7]));
+                acc[8] = fma(QCz, v12_0_0, fma(WQz, v12_0_1, fma(1.0 * oo2ze, v4_0_1, acc[8])));
+                acc[9] = fma(QCx, v13_0_0, fma(WQx, v13_0_1, fma(1.0 * oo2ze, v7_0_1, acc[9])));
+                acc[10] = fma(QCy, v13_0_0, fma(WQy, v13_0_1, fma(2.0 * oo2ze, v5_0_1, acc[10])));
+                acc[11] = fma(QCz, v13_0_0, fma(WQz, v13_0_1, acc[11]));
+                acc[12] = fma(QCx, v14_0_0, fma(WQx, v14_0_1, fma(1.0 * oo2ze, v9_0_1, acc[12])));
+                acc[13] = fma(QCy, v14_0_0, fma(WQy, v14_0_1, acc[13]));
+                acc[14] = fma(QCz, v14_0_0, fma(WQz, v14_0_1, fma(2.0 * oo2ze, v6_0_1, acc[14])));
+                acc[15] = fma(QCx, v15_0_0, fma(WQx, v15_0_1, fma(1.0 * oo2ze, v8_0_1, acc[15])));
+                acc[16] = fma(QCy, v15_0_0, fma(WQy, v15_0_1, fma(1.0 * oo2ze, v6_0_1, acc[16])));
+                acc[17] = fma(QCz, v15_0_0, fma(WQz, v15_0_1, fma(1.0 * oo2ze, v5_0_1, acc[17])));
+                acc[18] = fma(QCx, v16_0_0, fma(WQx, v16_0_1, acc[18]));
+                acc[19] = fma(QCy, v16_0_0, fma(WQy, v16_0_1, fma(3.0 * oo2ze, v7_0_1, acc[19])));
+                acc[20] = fma(QCz, v16_0_0, fma(WQz, v16_0_1, acc[20]));
+                acc[21] = fma(QCx, v17_0_0, fma(WQx, v17_0_1, acc[21]));
+                acc[22] = fma(QCy, v17_0_0, fma(WQy, v17_0_1, fma(2.0 * oo2ze, v8_0_1, acc[22])));
+                acc[23] = fma(QCz, v17_0_0, fma(WQz, v17_0_1, fma(1.0 * oo2ze, v7_0_1, acc[23])));
+                acc[24] = fma(QCx, v18_0_0, fma(WQx, v18_0_1, acc[24]));
+                acc[25] = fma(QCy, v18_0_0, fma(WQy, v18_0_1, fma(1.0 * oo2ze, v9_0_1, acc[25])));
+                acc[26] = fma(QCz, v18_0_0, fma(WQz, v18_0_1, fma(2.0 * oo2ze, v8_0_1, acc[26])));
+                acc[27] = fma(QCx, v19_0_0, fma(WQx, v19_0_1, acc[27]));
+                acc[28] = fma(QCy, v19_0_0, fma(WQy, v19_0_1, acc[28]));
+                acc[29] = fma(QCz, v19_0_0, fma(WQz, v19_0_1, fma(3.0 * oo2ze, v9_0_1, acc[29])));
+                acc[30] = fma(QCx, v20_0_0, fma(WQx, v20_0_1, fma(4.0 * oo2ze, v10_0_1, acc[30])));
+                acc[31] = fma(QCy, v20_0_0, fma(WQy, v20_0_1, acc[31]));
+                acc[32] = fma(QCz, v20_0_0, fma(WQz, v20_0_1, acc[32]));
+                acc[33] = fma(QCx, v21_0_0, fma(WQx, v21_0_1, fma(3.0 * oo2ze, v11_0_1, acc[33])));
+                acc[34] = fma(QCy, v21_0_0, fma(WQy, v21_0_1, fma(1.0 * oo2ze, v10_0_1, acc[34])));
+                acc[35] = fma(QCz, v21_0_0, fma(WQz, v21_0_1, acc[35]));
+                acc[36] = fma(QCx, v22_0_0, fma(WQx, v22_0_1, fma(3.0 * oo2ze, v12_0_1, acc[36])));
+                acc[37] = fma(QCy, v22_0_0, fma(WQy, v22_0_1, acc[37]));
+                acc[38] = fma(QCz, v22_0_0, fma(WQz, v22_0_1, fma(1.0 * oo2ze, v10_0_1, acc[38])));
+                acc[39] = fma(QCx, v23_0_0, fma(WQx, v23_0_1, fma(2.0 * oo2ze, v13_0_1, acc[39])));
+                acc[40] = fma(QCy, v23_0_0, fma(WQy, v23_0_1, fma(2.0 * oo2ze, v11_0_1, acc[40])));
+                acc[41] = fma(QCz, v23_0_0, fma(WQz, v23_0_1, acc[41]));
+                acc[42] = fma(QCx, v24_0_0, fma(WQx, v24_0_1, fma(2.0 * oo2ze, v15_0_1, acc[42])));
+                acc[43] = fma(QCy, v24_0_0, fma(WQy, v24_0_1, fma(1.0 * oo2ze, v12_0_1, acc[43])));
+                acc[44] = fma(QCz, v24_0_0, fma(WQz, v24_0_1, fma(1.0 * oo2ze, v11_0_1, acc[44])));
+                acc[45] = fma(QCx, v25_0_0, fma(WQx, v25_0_1, fma(2.0 * oo2ze, v14_0_1, acc[45])));
+                acc[46] = fma(QCy, v25_0_0, fma(WQy, v25_0_1, acc[46]));
+                acc[47] = fma(QCz, v25_0_0, fma(WQz, v25_0_1, fma(2.0 * oo2ze, v12_0_1, acc[47])));
+                acc[48] = fma(QCx, v26_0_0, fma(WQx, v26_0_1, fma(1.0 * oo2ze, v16_0_1, acc[48])));
+                acc[49] = fma(QCy, v26_0_0, fma(WQy, v26_0_1, fma(3.0 * oo2ze, v13_0_1, acc[49])));
+                acc[50] = fma(QCz, v26_0_0, fma(WQz, v26_0_1, acc[50]));
+                acc[51] = fma(QCx, v27_0_0, fma(WQx, v27_0_1, fma(1.0 * oo2ze, v17_0_1, acc[51])));
+                acc[52] = fma(QCy, v27_0_0, fma(WQy, v27_0_1, fma(2.0 * oo2ze, v15_0_1, acc[52])));
+                acc[53] = fma(QCz, v27_0_0, fma(WQz, v27_0_1, fma(1.0 * oo2ze, v13_0_1, acc[53])));
+                acc[54] = fma(QCx, v28_0_0, fma(WQx, v28_0_1, fma(1.0 * oo2ze, v18_0_1, acc[54])));
+                acc[55] = fma(QCy, v28_0_0, fma(WQy, v28_0_1, fma(1.0 * oo2ze, v14_0_1, acc[55])));
+                acc[56] = fma(QCz, v28_0_0, fma(WQz, v28_0_1, fma(2.0 * oo2ze, v15_0_1, acc[56])));
+                acc[57] = fma(QCx, v29_0_0, fma(WQx, v29_0_1, fma(1.0 * oo2ze, v19_0_1, acc[57])));
+                acc[58] = fma(QCy, v29_0_0, fma(WQy, v29_0_1, acc[58]));
+                acc[59] = fma(QCz, v29_0_0, fma(WQz, v29_0_1, fma(3.0 * oo2ze, v14_0_1, acc[59])));
+                acc[60] = fma(QCx, v30_0_0, fma(WQx, v30_0_1, acc[60]));
+                acc[61] = fma(QCy, v30_0_0, fma(WQy, v30_0_1, fma(4.0 * oo2ze, v16_0_1, acc[61])));
+                acc[62] = fma(QCz, v30_0_0, fma(WQz, v30_0_1, acc[62]));
+                acc[63] = fma(QCx, v31_0_0, fma(WQx, v31_0_1, acc[63]));
+                acc[64] = fma(QCy, v31_0_0, fma(WQy, v31_0_1, fma(3.0 * oo2ze, v17_0_1, acc[64])));
+                acc[65] = fma(QCz, v31_0_0, fma(WQz, v31_0_1, fma(1.0 * oo2ze, v16_0_1, acc[65])));
+                acc[66] = fma(QCx, v32_0_0, fma(WQx, v32_0_1, acc[66]));
+                acc[67] = fma(QCy, v32_0_0, fma(WQy, v32_0_1, fma(2.0 * oo2ze, v18_0_1, acc[67])));
+                acc[68] = fma(QCz, v32_0_0, fma(WQz, v32_0_1, fma(2.0 * oo2ze, v17_0_1, acc[68])));
+                acc[69] = fma(QCx, v33_0_0, fma(WQx, v33_0_1, acc[69]));
+                acc[70] = fma(QCy, v33_0_0, fma(WQy, v33_0_1, fma(1.0 * oo2ze, v19_0_1, acc[70])));
+                acc[71] = fma(QCz, v33_0_0, fma(WQz, v33_0_1, fma(3.0 * oo2ze, v18_0_1, acc[71])));
+                acc[72] = fma(QCx, v34_0_0, fma(WQx, v34_0_1, acc[72]));
+                acc[73] = fma(QCy, v34_0_0, fma(WQy, v34_0_1, acc[73]));
+                acc[74] = fma(QCz, v34_0_0, fma(WQz, v34_0_1, fma(4.0 * oo2ze, v19_0_1, acc[74])));
+                acc[75] = fma(QCx, v35_0_0, fma(WQx, v35_0_1, fma(5.0 * oo2ze, v20_0_1, acc[75])));
+                acc[76] = fma(QCy, v35_0_0, fma(WQy, v35_0_1, acc[76]));
+                acc[77] = fma(QCz, v35_0_0, fma(WQz, v35_0_1, acc[77]));
+                acc[78] = fma(QCx, v36_0_0, fma(WQx, v36_0_1, fma(4.0 * oo2ze, v21_0_1, acc[78])));
+                acc[79] = fma(QCy, v36_0_0, fma(WQy, v36_0_1, fma(1.0 * oo2ze, v20_0_1, acc[79])));
+                acc[80] = fma(QCz, v36_0_0, fma(WQz, v36_0_1, acc[80]));
+                acc[81] = fma(QCx, v37_0_0, fma(WQx, v37_0_1, fma(4.0 * oo2ze, v22_0_1, acc[81])));
+                acc[82] = fma(QCy, v37_0_0, fma(WQy, v37_0_1, acc[82]));
+                acc[83] = fma(QCz, v37_0_0, fma(WQz, v37_0_1, fma(1.0 * oo2ze, v20_0_1, acc[83])));
+                acc[84] = fma(QCx, v38_0_0, fma(WQx, v38_0_1, fma(3.0 * oo2ze, v23_0_1, acc[84])));
+                acc[85] = fma(QCy, v38_0_0, fma(WQy, v38_0_1, fma(2.0 * oo2ze, v21_0_1, acc[85])));
+                acc[86] = fma(QCz, v38_0_0, fma(WQz, v38_0_1, acc[86]));
+                acc[87] = fma(QCx, v39_0_0, fma(WQx, v39_0_1, fma(3.0 * oo2ze, v24_0_1, acc[87])));
+                acc[88] = fma(QCy, v39_0_0, fma(WQy, v39_0_1, fma(1.0 * oo2ze, v22_0_1, acc[88])));
+                acc[89] = fma(QCz, v39_0_0, fma(WQz, v39_0_1, fma(1.0 * oo2ze, v21_0_1, acc[89])));
+                acc[90] = fma(QCx, v40_0_0, fma(WQx, v40_0_1, fma(3.0 * oo2ze, v25_0_1, acc[90])));
+                acc[91] = fma(QCy, v40_0_0, fma(WQy, v40_0_1, acc[91]));
+                acc[92] = fma(QCz, v40_0_0, fma(WQz, v40_0_1, fma(2.0 * oo2ze, v22_0_1, acc[92])));
+                acc[93] = fma(QCx, v41_0_0, fma(WQx, v41_0_1, fma(2.0 * oo2ze, v26_0_1, acc[93])));
+                acc[94] = fma(QCy, v41_0_0, fma(WQy, v41_0_1, fma(3.0 * oo2ze, v23_0_1, acc[94])));
+                acc[95] = fma(QCz, v41_0_0, fma(WQz, v41_0_1, acc[95]));
+                acc[96] = fma(QCx, v42_0_0, fma(WQx, v42_0_1, fma(2.0 * oo2ze, v27_0_1, acc[96])));
+                acc[97] = fma(QCy, v42_0_0, fma(WQy, v42_0_1, fma(2.0 * oo2ze, v24_0_1, acc[97])));
+                acc[98] = fma(QCz, v42_0_0, fma(WQz, v42_0_1, fma(1.0 * oo2ze, v23_0_1, acc[98])));
+                acc[99] = fma(QCx, v43_0_0, fma(WQx, v43_0_1, fma(2.0 * oo2ze, v28_0_1, acc[99])));
+                acc[100] = fma(QCy, v43_0_0, fma(WQy, v43_0_1, fma(1.0 * oo2ze, v25_0_1, acc[100])));
+                acc[101] = fma(QCz, v43_0_0, fma(WQz, v43_0_1, fma(2.0 * oo2ze, v24_0_1, acc[101])));
+                acc[102] = fma(QCx, v44_0_0, fma(WQx, v44_0_1, fma(2.0 * oo2ze, v29_0_1, acc[102])));
+                acc[103] = fma(QCy, v44_0_0, fma(WQy, v44_0_1, acc[103]));
+                acc[104] = fma(QCz, v44_0_0, fma(WQz, v44_0_1, fma(3.0 * oo2ze, v25_0_1, acc[104])));
+                acc[105] = fma(QCx, v45_0_0, fma(WQx, v45_0_1, fma(1.0 * oo2ze, v30_0_1, acc[105])));
+                acc[106] = fma(QCy, v45_0_0, fma(WQy, v45_0_1, fma(4.0 * oo2ze, v26_0_1, acc[106])));
+                acc[107] = fma(QCz, v45_0_0, fma(WQz, v45_0_1, acc[107]));
+                acc[108] = fma(QCx, v46_0_0, fma(WQx, v46_0_1, fma(1.0 * oo2ze, v31_0_1, acc[108])));
+                acc[109] = fma(QCy, v46_0_0, fma(WQy, v46_0_1, fma(3.0 * oo2ze, v27_0_1, acc[109])));
+                acc[110] = fma(QCz, v46_0_0, fma(WQz, v46_0_1, fma(1.0 * oo2ze, v26_0_1, acc[110])));
+                acc[111] = fma(QCx, v47_0_0, fma(WQx, v47_0_1, fma(1.0 * oo2ze, v32_0_1, acc[111])));
+                acc[112] = fma(QCy, v47_0_0, fma(WQy, v47_0_1, fma(2.0 * oo2ze, v28_0_1, acc[112])));
+                acc[113] = fma(QCz, v47_0_0, fma(WQz, v47_0_1, fma(2.0 * oo2ze, v27_0_1, acc[113])));
+                acc[114] = fma(QCx, v48_0_0, fma(WQx, v48_0_1, fma(1.0 * oo2ze, v33_0_1, acc[114])));
+                acc[115] = fma(QCy, v48_0_0, fma(WQy, v48_0_1, fma(1.0 * oo2ze, v29_0_1, acc[115])));
+                acc[116] = fma(QCz, v48_0_0, fma(WQz, v48_0_1, fma(3.0 * oo2ze, v28_0_1, acc[116])));
+                acc[117] = fma(QCx, v49_0_0, fma(WQx, v49_0_1, fma(1.0 * oo2ze, v34_0_1, acc[117])));
+                acc[118] = fma(QCy, v49_0_0, fma(WQy, v49_0_1, acc[118]));
+                acc[119] = fma(QCz, v49_0_0, fma(WQz, v49_0_1, fma(4.0 * oo2ze, v29_0_1, acc[119])));
+                acc[120] = fma(QCx, v50_0_0, fma(WQx, v50_0_1, acc[120]));
+                acc[121] = fma(QCy, v50_0_0, fma(WQy, v50_0_1, fma(5.0 * oo2ze, v30_0_1, acc[121])));
+                acc[122] = fma(QCz, v50_0_0, fma(WQz, v50_0_1, acc[122]));
+                acc[123] = fma(QCx, v51_0_0, fma(WQx, v51_0_1, acc[123]));
+                acc[124] = fma(QCy, v51_0_0, fma(WQy, v51_0_1, fma(4.0 * oo2ze, v31_0_1, acc[124])));
+                acc[125] = fma(QCz, v51_0_0, fma(WQz, v51_0_1, fma(1.0 * oo2ze, v30_0_1, acc[125])));
+                acc[126] = fma(QCx, v52_0_0, fma(WQx, v52_0_1, acc[126]));
+                acc[127] = fma(QCy, v52_0_0, fma(WQy, v52_0_1, fma(3.0 * oo2ze, v32_0_1, acc[127])));
+                acc[128] = fma(QCz, v52_0_0, fma(WQz, v52_0_1, fma(2.0 * oo2ze, v31_0_1, acc[128])));
+                acc[129] = fma(QCx, v53_0_0, fma(WQx, v53_0_1, acc[129]));
+                acc[130] = fma(QCy, v53_0_0, fma(WQy, v53_0_1, fma(2.0 * oo2ze, v33_0_1, acc[130])));
+                acc[131] = fma(QCz, v53_0_0, fma(WQz, v53_0_1, fma(3.0 * oo2ze, v32_0_1, acc[131])));
+                acc[132] = fma(QCx, v54_0_0, fma(WQx, v54_0_1, acc[132]));
+                acc[133] = fma(QCy, v54_0_0, fma(WQy, v54_0_1, fma(1.0 * oo2ze, v34_0_1, acc[133])));
+                acc[134] = fma(QCz, v54_0_0, fma(WQz, v54_0_1, fma(4.0 * oo2ze, v33_0_1, acc[134])));
+                acc[135] = fma(QCx, v55_0_0, fma(WQx, v55_0_1, acc[135]));
+                acc[136] = fma(QCy, v55_0_0, fma(WQy, v55_0_1, acc[136]));
+                acc[137] = fma(QCz, v55_0_0, fma(WQz, v55_0_1, fma(5.0 * oo2ze, v34_0_1, acc[137])));
+            } else {
+                const VT v10_1_0 = QCx * v10_0_0 + WQx * v10_0_1 + (VT)3.0 * oo2ze * v4_0_1;
+                acc[0] += (double)v10_1_0;
+                const VT v10_2_0 = QCy * v10_0_0 + WQy * v10_0_1;
+                acc[1] += (double)v10_2_0;
+                const VT v10_3_0 = QCz * v10_0_0 + WQz * v10_0_1;
+                acc[2] += (double)v10_3_0;
+                const VT v11_1_0 = QCx * v11_0_0 + WQx * v11_0_1 + (VT)2.0 * oo2ze * v5_0_1;
+                acc[3] += (double)v11_1_0;
+                const VT v11_2_0 = QCy * v11_0_0 + WQy * v11_0_1 + (VT)1.0 * oo2ze * v4_0_1;
+                acc[4] += (double)v11_2_0;
+                const VT v11_3_0 = QCz * v11_0_0 + WQz * v11_0_1;
+                acc[5] += (double)v11_3_0;
+                const VT v12_1_0 = QCx * v12_0_0 + WQx * v12_0_1 + (VT)2.0 * oo2ze * v6_0_1;
+                acc[6] += (double)v12_1_0;
+                const VT v12_2_0 = QCy * v12_0_0 + WQy * v12_0_1;
+                acc[7] += (double)v12_2_0;
+                const VT v12_3_0 = QCz * v12_0_0 + WQz * v12_0_1 + (VT)1.0 * oo2ze * v4_0_1;
+                acc[8] += (double)v12_3_0;
+                const VT v13_1_0 = QCx * v13_0_0 + WQx * v13_0_1 + (VT)1.0 * oo2ze * v7_0_1;
+                acc[9] += (double)v13_1_0;
+                const VT v13_2_0 = QCy * v13_0_0 + WQy * v13_0_1 + (VT)2.0 * oo2ze * v5_0_1;
+                acc[10] += (double)v13_2_0;
+                const VT v13_3_0 = QCz * v13_0_0 + WQz * v13_0_1;
+                acc[11] += (double)v13_3_0;
+                const VT v14_1_0 = QCx * v14_0_0 + WQx * v14_0_1 + (VT)1.0 * oo2ze * v9_0_1;
+                acc[12] += (double)v14_1_0;
+                const VT v14_2_0 = QCy * v14_0_0 + WQy * v14_0_1;
+                acc[13] += (double)v14_2_0;
+                const VT v14_3_0 = QCz * v14_0_0 + WQz * v14_0_1 + (VT)2.0 * oo2ze * v6_0_1;
+                acc[14] += (double)v14_3_0;
+                const VT v15_1_0 = QCx * v15_0_0 + WQx * v15_0_1 + (VT)1.0 * oo2ze * v8_0_1;
+                acc[15] += (double)v15_1_0;
+                const VT v15_2_0 = QCy * v15_0_0 + WQy * v15_0_1 + (VT)1.0 * oo2ze * v6_0_1;
+                acc[16] += (double)v15_2_0;
+                const VT v15_3_0 = QCz * v15_0_0 + WQz * v15_0_1 + (VT)1.0 * oo2ze * v5_0_1;
+                acc[17] += (double)v15_3_0;
+                const VT v16_1_0 = QCx * v16_0_0 + WQx * v16_0_1;
+                acc[18] += (double)v16_1_0;
+                const VT v16_2_0 = QCy * v16_0_0 + WQy * v16_0_1 + (VT)3.0 * oo2ze * v7_0_1;
+                acc[19] += (double)v16_2_0;
+                const VT v16_3_0 = QCz * v16_0_0 + WQz * v16_0_1;
+                acc[20] += (double)v16_3_0;
+                const VT v17_1_0 = QCx * v17_0_0 + WQx * v17_0_1;
+                acc[21] += (double)v17_1_0;
+                const VT v17_2_0 = QCy * v17_0_0 + WQy * v17_0_1 + (VT)2.0 * oo2ze * v8_0_1;
+                acc[22] += (double)v17_2_0;
+                const VT v17_3_0 = QCz * v17_0_0 + WQz * v17_0_1 + (VT)1.0 * oo2ze * v7_0_1;
+                acc[23] += (double)v17_3_0;
+                const VT v18_1_0 = QCx * v18_0_0 + WQx * v18_0_1;
+                acc[24] += (double)v18_1_0;
+                const VT v18_2_0 = QCy * v18_0_0 + WQy * v18_0_1 + (VT)1.0 * oo2ze * v9_0_1;
+                acc[25] += (double)v18_2_0;
+                const VT v18_3_0 = QCz * v18_0_0 + WQz * v18_0_1 + (VT)2.0 * oo2ze * v8_0_1;
+                acc[26] += (double)v18_3_0;
+                const VT v19_1_0 = QCx * v19_0_0 + WQx * v19_0_1;
+                acc[27] += (double)v19_1_0;
+                const VT v19_2_0 = QCy * v19_0_0 + WQy * v19_0_1;
+                acc[28] += (double)v19_2_0;
+                const VT v19_3_0 = QCz * v19_0_0 + WQz * v19_0_1 + (VT)3.0 * oo2ze * v9_0_1;
+                acc[29] += (double)v19_3_0;
+                const VT v20_1_0 = QCx * v20_0_0 + WQx * v20_0_1 + (VT)4.0 * oo2ze * v10_0_1;
+                acc[30] += (double)v20_1_0;
+                const VT v20_2_0 = QCy * v20_0_0 + WQy * v20_0_1;
+                acc[31] += (double)v20_2_0;
+                const VT v20_3_0 = QCz * v20_0_0 + WQz * v20_0_1;
+                acc[32] += (double)v20_3_0;
+                const VT v21_1_0 = QCx * v21_0_0 + WQx * v21_0_1 + (VT)3.0 * oo2ze * v11_0_1;
+                acc[33] += (double)v21_1_0;
+                const VT v21_2_0 = QCy * v21_0_0 + WQy * v21_0_1 + (VT)1.0 * oo2ze * v10_0_1;
+                acc[34] += (double)v21_2_0;
+                const VT v21_3_0 = QCz * v21_0_0 + WQz * v21_0_1;
+                acc[35] += (double)v21_3_0;
+                const VT v22_1_0 = QCx * v22_0_0 + WQx * v22_0_1 + (VT)3.0 * oo2ze * v12_0_1;
+                acc[36] += (double)v22_1_0;
+                const VT v22_2_0 = QCy * v22_0_0 + WQy * v22_0_1;
+                acc[37] += (double)v22_2_0;
+                const VT v22_3_0 = QCz * v22_0_0 + WQz * v22_0_1 + (VT)1.0 * oo2ze * v10_0_1;
+                acc[38] += (double)v22_3_0;
+                const VT v23_1_0 = QCx * v23_0_0 + WQx * v23_0_1 + (VT)2.0 * oo2ze * v13_0_1;
+                acc[39] += (double)v23_1_0;
+                const VT v23_2_0 = QCy * v23_0_0 + WQy * v23_0_1 + (VT)2.0 * oo2ze * v11_0_1;
+                acc[40] += (double)v23_2_0;
+                const VT v23_3_0 = QCz * v23_0_0 + WQz * v23_0_1;
+                acc[41] += (double)v23_3_0;
+                const VT v24_1_0 = QCx * v24_0_0 + WQx * v24_0_1 + (VT)2.0 * oo2ze * v15_0_1;
+                acc[42] += (double)v24_1_0;
+                const VT v24_2_0 = QCy * v24_0_0 + WQy * v24_0_1 + (VT)1.0 * oo2ze * v12_0_1;
+                acc[43] += (double)v24_2_0;
+                const VT v24_3_0 = QCz * v24_0_0 + WQz * v24_0_1 + (VT)1.0 * oo2ze * v11_0_1;
+                acc[44] += (double)v24_3_0;
+                const VT v25_1_0 = QCx * v25_0_0 + WQx * v25_0_1 + (VT)2.0 * oo2ze * v14_0_1;
+                acc[45] += (double)v25_1_0;
+                const VT v25_2_0 = QCy * v25_0_0 + WQy * v25_0_1;
+                acc[46] += (double)v25_2_0;
+                const VT v25_3_0 = QCz * v25_0_0 + WQz * v25_0_1 + (VT)2.0 * oo2ze * v12_0_1;
+                acc[47] += (double)v25_3_0;
+                const VT v26_1_0 = QCx * v26_0_0 + WQx * v26_0_1 + (VT)1.0 * oo2ze * v16_0_1;
+                acc[48] += (double)v26_1_0;
+                const VT v26_2_0 = QCy * v26_0_0 + WQy * v26_0_1 + (VT)3.0 * oo2ze * v13_0_1;
+                acc[49] += (double)v26_2_0;
+                const VT v26_3_0 = QCz * v26_0_0 + WQz * v26_0_1;
+                acc[50] += (double)v26_3_0;
+                const VT v27_1_0 = QCx * v27_0_0 + WQx * v27_0_1 + (VT)1.0 * oo2ze * v17_0_1;
+                acc[51] += (double)v27_1_0;
+                const VT v27_2_0 = QCy * v27_0_0 + WQy * v27_0_1 + (VT)2.0 * oo2ze * v15_0_1;
+                acc[52] += (double)v27_2_0;
+                const VT v27_3_0 = QCz * v27_0_0 + WQz * v27_0_1 + (VT)1.0 * oo2ze * v13_0_1;
+                acc[53] += (double)v27_3_0;
+                const VT v28_1_0 = QCx * v28_0_0 + WQx * v28_0_1 + (VT)1.0 * oo2ze * v18_0_1;
+                acc[54] += (double)v28_1_0;
+                const VT v28_2_0 = QCy * v28_0_0 + WQy * v28_0_1 + (VT)1.0 * oo2ze * v14_0_1;
+                acc[55] += (double)v28_2_0;
+                const VT v28_3_0 = QCz * v28_0_0 + WQz * v28_0_1 + (VT)2.0 * oo2ze * v15_0_1;
+                acc[56] += (double)v28_3_0;
+                const VT v29_1_0 = QCx * v29_0_0 + WQx * v29_0_1 + (VT)1.0 * oo2ze * v19_0_1;
+                acc[57] += (double)v29_1_0;
+                const VT v29_2_0 = QCy * v29_0_0 + WQy * v29_0_1;
+                acc[58] += (double)v29_2_0;
+                const VT v29_3_0 = QCz * v29_0_0 + WQz * v29_0_1 + (VT)3.0 * oo2ze * v14_0_1;
+                acc[59] += (double)v29_3_0;
+                const VT v30_1_0 = QCx * v30_0_0 + WQx * v30_0_1;
+                acc[60] += (double)v30_1_0;
+                const VT v30_2_0 = QCy * v30_0_0 + WQy * v30_0_1 + (VT)4.0 * oo2ze * v16_0_1;
+                acc[61] += (double)v30_2_0;
+                const VT v30_3_0 = QCz * v30_0_0 + WQz * v30_0_1;
+                acc[62] += (double)v30_3_0;
+                const VT v31_1_0 = QCx * v31_0_0 + WQx * v31_0_1;
+                acc[63] += (double)v31_1_0;
+                const VT v31_2_0 = QCy * v31_0_0 + WQy * v31_0_1 + (VT)3.0 * oo2ze * v17_0_1;
+                acc[64] += (double)v31_2_0;
+                const VT v31_3_0 = QCz * v31_0_0 + WQz * v31_0_1 + (VT)1.0 * oo2ze * v16_0_1;
+                acc[65] += (double)v31_3_0;
+                const VT v32_1_0 = QCx * v32_0_0 + WQx * v32_0_1;
+                acc[66] += (double)v32_1_0;
+                const VT v32_2_0 = QCy * v32_0_0 + WQy * v32_0_1 + (VT)2.0 * oo2ze * v18_0_1;
+                acc[67] += (double)v32_2_0;
+                const VT v32_3_0 = QCz * v32_0_0 + WQz * v32_0_1 + (VT)2.0 * oo2ze * v17_0_1;
+                acc[68] += (double)v32_3_0;
+                const VT v33_1_0 = QCx * v33_0_0 + WQx * v33_0_1;
+                acc[69] += (double)v33_1_0;
+                const VT v33_2_0 = QCy * v33_0_0 + WQy * v33_0_1 + (VT)1.0 * oo2ze * v19_0_1;
+                acc[70] += (double)v33_2_0;
+                const VT v33_3_0 = QCz * v33_0_0 + WQz * v33_0_1 + (VT)3.0 * oo2ze * v18_0_1;
+                acc[71] += (double)v33_3_0;
+                const VT v34_1_0 = QCx * v34_0_0 + WQx * v34_0_1;
+                acc[72] += (double)v34_1_0;
+                const VT v34_2_0 = QCy * v34_0_0 + WQy * v34_0_1;
+                acc[73] += (double)v34_2_0;
+                const VT v34_3_0 = QCz * v34_0_0 + WQz * v34_0_1 + (VT)4.0 * oo2ze * v19_0_1;
+                acc[74] += (double)v34_3_0;
+                const VT v35_1_0 = QCx * v35_0_0 + WQx * v35_0_1 + (VT)5.0 * oo2ze * v20_0_1;
+                acc[75] += (double)v35_1_0;
+                const VT v35_2_0 = QCy * v35_0_0 + WQy * v35_0_1;
+                acc[76] += (double)v35_2_0;
+                const VT v35_3_0 = QCz * v35_0_0 + WQz * v35_0_1;
+                acc[77] += (double)v35_3_0;
+                const VT v36_1_0 = QCx * v36_0_0 + WQx * v36_0_1 + (VT)4.0 * oo2ze * v21_0_1;
+                acc[78] += (double)v36_1_0;
+                const VT v36_2_0 = QCy * v36_0_0 + WQy * v36_0_1 + (VT)1.0 * oo2ze * v20_0_1;
+                acc[79] += (double)v36_2_0;
+                const VT v36_3_0 = QCz * v36_0_0 + WQz * v36_0_1;
+                acc[80] += (double)v36_3_0;
+                const VT v37_1_0 = QCx * v37_0_0 + WQx * v37_0_1 + (VT)4.0 * oo2ze * v22_0_1;
+                acc[81] += (double)v37_1_0;
+                const VT v37_2_0 = QCy * v37_0_0 + WQy * v37_0_1;
+                acc[82] += (double)v37_2_0;
+                const VT v37_3_0 = QCz * v37_0_0 + WQz * v37_0_1 + (VT)1.0 * oo2ze * v20_0_1;
+                acc[83] += (double)v37_3_0;
+                const VT v38_1_0 = QCx * v38_0_0 + WQx * v38_0_1 + (VT)3.0 * oo2ze * v23_0_1;
+                acc[84] += (double)v38_1_0;
+                const VT v38_2_0 = QCy * v38_0_0 + WQy * v38_0_1 + (VT)2.0 * oo2ze * v21_0_1;
+                acc[85] += (double)v38_2_0;
+                const VT v38_3_0 = QCz * v38_0_0 + WQz * v38_0_1;
+                acc[86] += (double)v38_3_0;
+                const VT v39_1_0 = QCx * v39_0_0 + WQx * v39_0_1 + (VT)3.0 * oo2ze * v24_0_1;
+                acc[87] += (double)v39_1_0;
+                const VT v39_2_0 = QCy * v39_0_0 + WQy * v39_0_1 + (VT)1.0 * oo2ze * v22_0_1;
+                acc[88] += (double)v39_2_0;
+                const VT v39_3_0 = QCz * v39_0_0 + WQz * v39_0_1 + (VT)1.0 * oo2ze * v21_0_1;
+                acc[89] += (double)v39_3_0;
+                const VT v40_1_0 = QCx * v40_0_0 + WQx * v40_0_1 + (VT)3.0 * oo2ze * v25_0_1;
+                acc[90] += (double)v40_1_0;
+                const VT v40_2_0 = QCy * v40_0_0 + WQy * v40_0_1;
+                acc[91] += (double)v40_2_0;
+                const VT v40_3_0 = QCz * v40_0_0 + WQz * v40_0_1 + (VT)2.0 * oo2ze * v22_0_1;
+                acc[92] += (double)v40_3_0;
+                const VT v41_1_0 = QCx * v41_0_0 + WQx * v41_0_1 + (VT)2.0 * oo2ze * v26_0_1;
+                acc[93] += (double)v41_1_0;
+                const VT v41_2_0 = QCy * v41_0_0 + WQy * v41_0_1 + (VT)3.0 * oo2ze * v23_0_1;
+                acc[94] += (double)v41_2_0;
+                const VT v41_3_0 = QCz * v41_0_0 + WQz * v41_0_1;
+                acc[95] += (double)v41_3_0;
+                const VT v42_1_0 = QCx * v42_0_0 + WQx * v42_0_1 + (VT)2.0 * oo2ze * v27_0_1;
+                acc[96] += (double)v42_1_0;
+                const VT v42_2_0 = QCy * v42_0_0 + WQy * v42_0_1 + (VT)2.0 * oo2ze * v24_0_1;
+                acc[97] += (double)v42_2_0;
+                const VT v42_3_0 = QCz * v42_0_0 + WQz * v42_0_1 + (VT)1.0 * oo2ze * v23_0_1;
+                acc[98] += (double)v42_3_0;
+                const VT v43_1_0 = QCx * v43_0_0 + WQx * v43_0_1 + (VT)2.0 * oo2ze * v28_0_1;
+                acc[99] += (double)v43_1_0;
+                const VT v43_2_0 = QCy * v43_0_0 + WQy * v43_0_1 + (VT)1.0 * oo2ze * v25_0_1;
+                acc[100] += (double)v43_2_0;
+                const VT v43_3_0 = QCz * v43_0_0 + WQz * v43_0_1 + (VT)2.0 * oo2ze * v24_0_1;
+                acc[101] += (double)v43_3_0;
+                const VT v44_1_0 = QCx * v44_0_0 + WQx * v44_0_1 + (VT)2.0 * oo2ze * v29_0_1;
+                acc[102] += (double)v44_1_0;
+                const VT v44_2_0 = QCy * v44_0_0 + WQy * v44_0_1;
+                acc[103] += (double)v44_2_0;
+                const VT v44_3_0 = QCz * v44_0_0 + WQz * v44_0_1 + (VT)3.0 * oo2ze * v25_0_1;
+                acc[104] += (double)v44_3_0;
+                const VT v45_1_0 = QCx * v45_0_0 + WQx * v45_0_1 + (VT)1.0 * oo2ze * v30_0_1;
+                acc[105] += (double)v45_1_0;
+                const VT v45_2_0 = QCy * v45_0_0 + WQy * v45_0_1 + (VT)4.0 * oo2ze * v26_0_1;
+                acc[106] += (double)v45_2_0;
+                const VT v45_3_0 = QCz * v45_0_0 + WQz * v45_0_1;
+                acc[107] += (double)v45_3_0;
+                const VT v46_1_0 = QCx * v46_0_0 + WQx * v46_0_1 + (VT)1.0 * oo2ze * v31_0_1;
+                acc[108] += (double)v46_1_0;
+                const VT v46_2_0 = QCy * v46_0_0 + WQy * v46_0_1 + (VT)3.0 * oo2ze * v27_0_1;
+                acc[109] += (double)v46_2_0;
+                const VT v46_3_0 = QCz * v46_0_0 + WQz * v46_0_1 + (VT)1.0 * oo2ze * v26_0_1;
+                acc[110] += (double)v46_3_0;
+                const VT v47_1_0 = QCx * v47_0_0 + WQx * v47_0_1 + (VT)1.0 * oo2ze * v32_0_1;
+                acc[111] += (double)v47_1_0;
+                const VT v47_2_0 = QCy * v47_0_0 + WQy * v47_0_1 + (VT)2.0 * oo2ze * v28_0_1;
+                acc[112] += (double)v47_2_0;
+                const VT v47_3_0 = QCz * v47_0_0 + WQz * v47_0_1 + (VT)2.0 * oo2ze * v27_0_1;
+                acc[113] += (double)v47_3_0;
+                const VT v48_1_0 = QCx * v48_0_0 + WQx * v48_0_1 + (VT)1.0 * oo2ze * v33_0_1;
+                acc[114] += (double)v48_1_0;
+                const VT v48_2_0 = QCy * v48_0_0 + WQy * v48_0_1 + (VT)1.0 * oo2ze * v29_0_1;
+                acc[115] += (double)v48_2_0;
+                const VT v48_3_0 = QCz * v48_0_0 + WQz * v48_0_1 + (VT)3.0 * oo2ze * v28_0_1;
+                acc[116] += (double)v48_3_0;
+                const VT v49_1_0 = QCx * v49_0_0 + WQx * v49_0_1 + (VT)1.0 * oo2ze * v34_0_1;
+                acc[117] += (double)v49_1_0;
+                const VT v49_2_0 = QCy * v49_0_0 + WQy * v49_0_1;
+                acc[118] += (double)v49_2_0;
+                const VT v49_3_0 = QCz * v49_0_0 + WQz * v49_0_1 + (VT)4.0 * oo2ze * v29_0_1;
+                acc[119] += (double)v49_3_0;
+                const VT v50_1_0 = QCx * v50_0_0 + WQx * v50_0_1;
+                acc[120] += (double)v50_1_0;
+                const VT v50_2_0 = QCy * v50_0_0 + WQy * v50_0_1 + (VT)5.0 * oo2ze * v30_0_1;
+                acc[121] += (double)v50_2_0;
+                const VT v50_3_0 = QCz * v50_0_0 + WQz * v50_0_1;
+                acc[122] += (double)v50_3_0;
+                const VT v51_1_0 = QCx * v51_0_0 + WQx * v51_0_1;
+                acc[123] += (double)v51_1_0;
+                const VT v51_2_0 = QCy * v51_0_0 + WQy * v51_0_1 + (VT)4.0 * oo2ze * v31_0_1;
+                acc[124] += (double)v51_2_0;
+                const VT v51_3_0 = QCz * v51_0_0 + WQz * v51_0_1 + (VT)1.0 * oo2ze * v30_0_1;
+                acc[125] += (double)v51_3_0;
+                const VT v52_1_0 = QCx * v52_0_0 + WQx * v52_0_1;
+                acc[126] += (double)v52_1_0;
+                const VT v52_2_0 = QCy * v52_0_0 + WQy * v52_0_1 + (VT)3.0 * oo2ze * v32_0_1;
+                acc[127] += (double)v52_2_0;
+                const VT v52_3_0 = QCz * v52_0_0 + WQz * v52_0_1 + (VT)2.0 * oo2ze * v31_0_1;
+                acc[128] += (double)v52_3_0;
+                const VT v53_1_0 = QCx * v53_0_0 + WQx * v53_0_1;
+                acc[129] += (double)v53_1_0;
+                const VT v53_2_0 = QCy * v53_0_0 + WQy * v53_0_1 + (VT)2.0 * oo2ze * v33_0_1;
+                acc[130] += (double)v53_2_0;
+                const VT v53_3_0 = QCz * v53_0_0 + WQz * v53_0_1 + (VT)3.0 * oo2ze * v32_0_1;
+                acc[131] += (double)v53_3_0;
+                const VT v54_1_0 = QCx * v54_0_0 + WQx * v54_0_1;
+                acc[132] += (double)v54_1_0;
+                const VT v54_2_0 = QCy * v54_0_0 + WQy * v54_0_1 + (VT)1.0 * oo2ze * v34_0_1;
+                acc[133] += (double)v54_2_0;
+                const VT v54_3_0 = QCz * v54_0_0 + WQz * v54_0_1 + (VT)4.0 * oo2ze * v33_0_1;
+                acc[134] += (double)v54_3_0;
+                const VT v55_1_0 = QCx * v55_0_0 + WQx * v55_0_1;
+                acc[135] += (double)v55_1_0;
+                const VT v55_2_0 = QCy * v55_0_0 + WQy * v55_0_1;
+                acc[136] += (double)v55_2_0;
+                const VT v55_3_0 = QCz * v55_0_0 + WQz * v55_0_1 + (VT)5.0 * oo2ze * v34_0_1;
+                acc[137] += (double)v55_3_0;
+            }
         }
     }
 }

@@ -25,13 +25,13 @@ __device__ __forceinline__ void vrr_fdss(const PairTab &P, const BoysTab &B, int
             const double r = rsqrt(bra.zeta + ket.zeta);
             const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
-            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[6];
             boys_fm<5>(T, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
-            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
             const VT WQx = (VT)(zz * PQx), WQy = (VT)(zz * PQy), WQz = (VT)(zz * PQz);
             const VT oo2z = (VT)bra.oo2z, oo2e = (VT)ket.oo2z, oo2ze = (VT)(0.5 * r2);
@@ -144,73 +144,122 @@ __device__ __forceinline__ void vrr_fdss(const PairTab &P, const BoysTab &B, int
             const VT v33_0_1 = PAz * v18_0_1 + WPz * v18_0_2 + (VT)2.0 * oo2z * (v8_0_1 - rho_z * v8_0_2);
             const VT v34_0_0 = PAz * v19_0_0 + WPz * v19_0_1 + (VT)3.0 * oo2z * (v9_0_0 - rho_z * v9_0_1);
             const VT v34_0_1 = PAz * v19_0_1 + WPz * v19_0_2 + (VT)3.0 * oo2z * (v9_0_1 - rho_z * v9_0_2);
-            const VT v35_0_0 = PAx * v20_0_0 + WPx * v20_0_1 + (VT)4.0 * oo2z * (v10_0_0 - rho_z * v10_0_1);
-            const VT v36_0_0 = PAx * v21_0_0 + WPx * v21_0_1 + (VT)3.0 * oo2z * (v11_0_0 - rho_z * v11_0_1);
-            const VT v37_0_0 = PAx * v22_0_0 + WPx * v22_0_1 + (VT)3.0 * oo2z * (v12_0_0 - rho_z * v12_0_1);
-            const VT v38_0_0 = PAx * v23_0_0 + WPx * v23_0_1 + (VT)2.0 * oo2z * (v13_0_0 - rho_z * v13_0_1);
-            const VT v39_0_0 = PAx * v24_0_0 + WPx * v24_0_1 + (VT)2.0 * oo2z * (v15_0_0 - rho_z * v15_0_1);
-            const VT v40_0_0 = PAx * v25_0_0 + WPx * v25_0_1 + (VT)2.0 * oo2z * (v14_0_0 - rho_z * v14_0_1);
-            const VT v41_0_0 = PAy * v23_0_0 + WPy * v23_0_1 + (VT)2.0 * oo2z * (v11_0_0 - rho_z * v11_0_1);
-            const VT v42_0_0 = PAx * v27_0_0 + WPx * v27_0_1 + (VT)1.0 * oo2z * (v17_0_0 - rho_z * v17_0_1);
-            const VT v43_0_0 = PAx * v28_0_0 + WPx * v28_0_1 + (VT)1.0 * oo2z * (v18_0_0 - rho_z * v18_0_1);
-            const VT v44_0_0 = PAz * v25_0_0 + WPz * v25_0_1 + (VT)2.0 * oo2z * (v12_0_0 - rho_z * v12_0_1);
-            const VT v45_0_0 = PAy * v26_0_0 + WPy * v26_0_1 + (VT)3.0 * oo2z * (v13_0_0 - rho_z * v13_0_1);
-            const VT v46_0_0 = PAy * v27_0_0 + WPy * v27_0_1 + (VT)2.0 * oo2z * (v15_0_0 - rho_z * v15_0_1);
-            const VT v47_0_0 = PAy * v28_0_0 + WPy * v28_0_1 + (VT)1.0 * oo2z * (v14_0_0 - rho_z * v14_0_1);
-            const VT v48_0_0 = PAz * v28_0_0 + WPz * v28_0_1 + (VT)2.0 * oo2z * (v15_0_0 - rho_z * v15_0_1);
-            const VT v49_0_0 = PAz * v29_0_0 + WPz * v29_0_1 + (VT)3.0 * oo2z * (v14_0_0 - rho_z * v14_0_1);
-            const VT v50_0_0 = PAy * v30_0_0 + WPy * v30_0_1 + (VT)4.0 * oo2z * (v16_0_0 - rho_z * v16_0_1);
-            const VT v51_0_0 = PAy * v31_0_0 + WPy * v31_0_1 + (VT)3.0 * oo2z * (v17_0_0 - rho_z * v17_0_1);
-            const VT v52_0_0 = PAy * v32_0_0 + WPy * v32_0_1 + (VT)2.0 * oo2z * (v18_0_0 - rho_z * v18_0_1);
-            const VT v53_0_0 = PAz * v32_0_0 + WPz * v32_0_1 + (VT)2.0 * oo2z * (v17_0_0 - rho_z * v17_0_1);
-            const VT v54_0_0 = PAz * v33_0_0 + WPz * v33_0_1 + (VT)3.0 * oo2z * (v18_0_0 - rho_z * v18_0_1);
-            const VT v55_0_0 = PAz * v34_0_0 + WPz * v34_0_1 + (VT)4.0 * oo2z * (v19_0_0 - rho_z * v19_0_1);
-            acc[0] += (double)v10_0_0;
-            acc[1] += (double)v11_0_0;
-            acc[2] += (double)v12_0_0;
-            acc[3] += (double)v13_0_0;
-            acc[4] += (double)v14_0_0;
-            acc[5] += (double)v15_0_0;
-            acc[6] += (double)v16_0_0;
-            acc[7] += (double)v17_0_0;
-            acc[8] += (double)v18_0_0;
-            acc[9] += (double)v19_0_0;
-            acc[10] += (double)v20_0_0;
-            acc[11] += (double)v21_0_0;
-            acc[12] += (double)v22_0_0;
-            acc[13] += (double)v23_0_0;
-            acc[14] += (double)v24_0_0;
-            acc[15] += (double)v25_0_0;
-            acc[16] += (double)v26_0_0;
-            acc[17] += (double)v27_0_0;
-            acc[18] += (double)v28_0_0;
-            acc[19] += (double)v29_0_0;
-            acc[20] += (double)v30_0_0;
-            acc[21] += (double)v31_0_0;
-            acc[22] += (double)v32_0_0;
-            acc[23] += (double)v33_0_0;
-            acc[24] += (double)v34_0_0;
-            acc[25] += (double)v35_0_0;
-            acc[26] += (double)v36_0_0;
-            acc[27] += (double)v37_0_0;
-            acc[28] += (double)v38_0_0;
-            acc[29] += (double)v39_0_0;
-            acc[30] += (double)v40_0_0;
-            acc[31] += (double)v41_0_0;
-            acc[32] += (double)v42_0_0;
-            acc[33] += (double)v43_0_0;
-            acc[34] += (double)v44_0_0;
-            acc[35] += (double)v45_0_0;
-            acc[36] += (double)v46_0_0;
-            acc[37] += (double)v47_0_0;
-            acc[38] += (double)v48_0_0;
-            acc[39] += (double)v49_0_0;
-            acc[40] += (double)v50_0_0;
-            acc[41] += (double)v51_0_0;
-            acc[42] += (double)v52_0_0;
-            acc[43] += (double)v53_0_0;
-            acc[44] += (double)v54_0_0;
-            acc[45] += (double)v55_0_0;
+            if constexpr (sizeof(VT) == 8) {
+                acc[0] += (double)v10_0_0;
+                acc[1] += (double)v11_0_0;
+                acc[2] += (double)v12_0_0;
+                acc[3] += (double)v13_0_0;
+                acc[4] += (double)v14_0_0;
+                acc[5] += (double)v15_0_0;
+                acc[6] += (double)v16_0_0;
+                acc[7] += (double)v17_0_0;
+                acc[8] += (double)v18_0_0;
+                acc[9] += (double)v19_0_0;
+                acc[10] += (double)v20_0_0;
+                acc[11] += (double)v21_0_0;
+                acc[12] += (double)v22_0_0;
+                acc[13] += (double)v23_0_0;
+                acc[14] += (double)v24_0_0;
+                acc[15] += (double)v25_0_0;
+                acc[16] += (double)v26_0_0;
+                acc[17] += (double)v27_0_0;
+                acc[18] += (double)v28_0_0;
+                acc[19] += (double)v29_0_0;
+                acc[20] += (double)v30_0_0;
+                acc[21] += (double)v31_0_0;
+                acc[22] += (double)v32_0_0;
+                acc[23] += (double)v33_0_0;
+                acc[24] += (double)v34_0_0;
+                acc[25] = fma(PAx, v20_0_0, fma(WPx, v20_0_1, fma(4.0 * oo2z, (v10_0_0 - rho_z * v10_0_1), acc[25])));
+                acc[26] = fma(PAx, v21_0_0, fma(WPx, v21_0_1, fma(3.0 * oo2z, (v11_0_0 - rho_z * v11_0_1), acc[26])));
+                acc[27] = fma(PAx, v22_0_0, fma(WPx, v22_0_1, fma(3.0 * oo2z, (v12_0_0 - rho_z * v12_0_1), acc[27])));
+                acc[28] = fma(PAx, v23_0_0, fma(WPx, v23_0_1, fma(2.0 * oo2z, (v13_0_0 - rho_z * v13_0_1), acc[28])));
+                acc[29] = fma(PAx, v24_0_0, fma(WPx, v24_0_1, fma(2.0 * oo2z, (v15_0_0 - rho_z * v15_0_1), acc[29])));
+                acc[30] = fma(PAx, v25_0_0, fma(WPx, v25_0_1, fma(2.0 * oo2z, (v14_0_0 - rho_z * v14_0_1), acc[30])));
+                acc[31] = fma(PAy, v23_0_0, fma(WPy, v23_0_1, fma(2.0 * oo2z, (v11_0_0 - rho_z * v11_0_1), acc[31])));
+                acc[32] = fma(PAx, v27_0_0, fma(WPx, v27_0_1, fma(1.0 * oo2z, (v17_0_0 - rho_z * v17_0_1), acc[32])));
+                acc[33] = fma(PAx, v28_0_0, fma(WPx, v28_0_1, fma(1.0 * oo2z, (v18_0_0 - rho_z * v18_0_1), acc[33])));
+                acc[34] = fma(PAz, v25_0_0, fma(WPz, v25_0_1, fma(2.0 * oo2z, (v12_0_0 - rho_z * v12_0_1), acc[34])));
+                acc[35] = fma(PAy, v26_0_0, fma(WPy, v26_0_1, fma(3.0 * oo2z, (v13_0_0 - rho_z * v13_0_1), acc[35])));
+                acc[36] = fma(PAy, v27_0_0, fma(WPy, v27_0_1, fma(2.0 * oo2z, (v15_0_0 - rho_z * v15_0_1), acc[36])));
+                acc[37] = fma(PAy, v28_0_0, fma(WPy, v28_0_1, fma(1.0 * oo2z, (v14_0_0 - rho_z * v14_0_1), acc[37])));
+                acc[38] = fma(PAz, v28_0_0, fma(WPz, v28_0_1, fma(2.0 * oo2z, (v15_0_0 - rho_z * v15_0_1), acc[38])));
+                acc[39] = fma(PAz, v29_0_0, fma(WPz, v29_0_1, fma(3.0 * oo2z, (v14_0_0 - rho_z * v14_0_1), acc[39])));
+                acc[40] = fma(PAy, v30_0_0, fma(WPy, v30_0_1, fma(4.0 * oo2z, (v16_0_0 - rho_z * v16_0_1), acc[40])));
+                acc[41] = fma(PAy, v31_0_0, fma(WPy, v31_0_1, fma(3.0 * oo2z, (v17_0_0 - rho_z * v17_0_1), acc[41])));
+                acc[42] = fma(PAy, v32_0_0, fma(WPy, v32_0_1, fma(2.0 * oo2z, (v18_0_0 - rho_z * v18_0_1), acc[42])));
+                acc[43] = fma(PAz, v32_0_0, fma(WPz, v32_0_1, fma(2.0 * oo2z, (v17_0_0 - rho_z * v17_0_1), acc[43])));
+                acc[44] = fma(PAz, v33_0_0, fma(WPz, v33_0_1, fma(3.0 * oo2z, (v18_0_0 - rho_z * v18_0_1), acc[44])));
+                acc[45] = fma(PAz, v34_0_0, fma(WPz, v34_0_1, fma(4.0 * oo2z, (v19_0_0 - rho_z * v19_0_1), acc[45])));
+            } else {
+                acc[0] += (double)v10_0_0;
+                acc[1] += (double)v11_0_0;
+                acc[2] += (double)v12_0_0;
+                acc[3] += (double)v13_0_0;
+                acc[4] += (double)v14_0_0;
+                acc[5] += (double)v15_0_0;
+                acc[6] += (double)v16_0_0;
+                acc[7] += (double)v17_0_0;
+                acc[8] += (double)v18_0_0;
+                acc[9] += (double)v19_0_0;
+                acc[10] += (double)v20_0_0;
+                acc[11] += (double)v21_0_0;
+                acc[12] += (double)v22_0_0;
+                acc[13] += (double)v23_0_0;
+                acc[14] += (double)v24_0_0;
+                acc[15] += (double)v25_0_0;
+                acc[16] += (double)v26_0_0;
+                acc[17] += (double)v27_0_0;
+                acc[18] += (double)v28_0_0;
+                acc[19] += (double)v29_0_0;
+                acc[20] += (double)v30_0_0;
+                acc[21] += (double)v31_0_0;
+                acc[22] += (double)v32_0_0;
+                acc[23] += (double)v33_0_0;
+                acc[24] += (double)v34_0_0;
+                const VT v35_0_0 = PAx * v20_0_0 + WPx * v20_0_1 + (VT)4.0 * oo2z * (v10_0_0 - rho_z * v10_0_1);
+                acc[25] += (double)v35_0_0;
+                const VT v36_0_0 = PAx * v21_0_0 + WPx * v21_0_1 + (VT)3.0 * oo2z * (v11_0_0 - rho_z * v11_0_1);
+                acc[26] += (double)v36_0_0;
+                const VT v37_0_0 = PAx * v22_0_0 + WPx * v22_0_1 + (VT)3.0 * oo2z * (v12_0_0 - rho_z * v12_0_1);
+                acc[27] += (double)v37_0_0;
+                const VT v38_0_0 = PAx * v23_0_0 + WPx * v23_0_1 + (VT)2.0 * oo2z * (v13_0_0 - rho_z * v13_0_1);
+                acc[28] += (double)v38_0_0;
+                const VT v39_0_0 = PAx * v24_0_0 + WPx * v24_0_1 + (VT)2.0 * oo2z * (v15_0_0 - rho_z * v15_0_1);
+                acc[29] += (double)v39_0_0;
+                const VT v40_0_0 = PAx * v25_0_0 + WPx * v25_0_1 + (VT)2.0 * oo2z * (v14_0_0 - rho_z * v14_0_1);
+                acc[30] += (double)v40_0_0;
+                const VT v41_0_0 = PAy * v23_0_0 + WPy * v23_0_1 + (VT)2.0 * oo2z * (v11_0_0 - rho_z * v11_0_1);
+                acc[31] += (double)v41_0_0;
+                const VT v42_0_0 = PAx * v27_0_0 + WPx * v27_0_1 + (VT)1.0 * oo2z * (v17_0_0 - rho_z * v17_0_1);
+                acc[32] += (double)v42_0_0;
+                const VT v43_0_0 = PAx * v28_0_0 + WPx * v28_0_1 + (VT)1.0 * oo2z * (v18_0_0 - rho_z * v18_0_1);
+                acc[33] += (double)v43_0_0;
+                const VT v44_0_0 = PAz * v25_0_0 + WPz * v25_0_1 + (VT)2.0 * oo2z * (v12_0_0 - rho_z * v12_0_1);
+                acc[34] += (double)v44_0_0;
+                const VT v45_0_0 = PAy * v26_0_0 + WPy * v26_0_1 + (VT)3.0 * oo2z * (v13_0_0 - rho_z * v13_0_1);
+                acc[35] += (double)v45_0_0;
+                const VT v46_0_0 = PAy * v27_0_0 + WPy * v27_0_1 + (VT)2.0 * oo2z * (v15_0_0 - rho_z * v15_0_1);
+                acc[36] += (double)v46_0_0;
+                const VT v47_0_0 = PAy * v28_0_0 + WPy * v28_0_1 + (VT)1.0 * oo2z * (v14_0_0 - rho_z * v14_0_1);
+                acc[37] += (double)v47_0_0;
+                const VT v48_0_0 = PAz * v28_0_0 + WPz * v28_0_1 + (VT)2.0 * oo2z * (v15_0_0 - rho_z * v15_0_1);
+                acc[38] += (double)v48_0_0;
+                const VT v49_0_0 = PAz * v29_0_0 + WPz * v29_0_1 + (VT)3.0 * oo2z * (v14_0_0 - rho_z * v14_0_1);
+                acc[39] += (double)v49_0_0;
+                const VT v50_0_0 = PAy * v30_0_0 + WPy * v30_0_1 + (VT)4.0 * oo2z * (v16_0_0 - rho_z * v16_0_1);
+                acc[40] += (double)v50_0_0;
+                const VT v51_0_0 = PAy * v31_0_0 + WPy * v31_0_1 + (VT)3.0 * oo2z * (v17_0_0 - rho_z * v17_0_1);
+                acc[41] += (double)v51_0_0;
+                const VT v52_0_0 = PAy * v32_0_0 + WPy * v32_0_1 + (VT)2.0 * oo2z * (v18_0_0 - rho_z * v18_0_1);
+                acc[42] += (double)v52_0_0;
+                const VT v53_0_0 = PAz * v32_0_0 + WPz * v32_0_1 + (VT)2.0 * oo2z * (v17_0_0 - rho_z * v17_0_1);
+                acc[43] += (double)v53_0_0;
+                const VT v54_0_0 = PAz * v33_0_0 + WPz * v33_0_1 + (VT)3.0 * oo2z * (v18_0_0 - rho_z * v18_0_1);
+                acc[44] += (double)v54_0_0;
+                const VT v55_0_0 = PAz * v34_0_0 + WPz * v34_0_1 + (VT)4.0 * oo2z * (v19_0_0 - rho_z * v19_0_1);
+                acc[45] += (double)v55_0_0;
+            }
         }
     }
 }

@@ -25,13 +25,13 @@ __device__ __forceinline__ void vrr_ffss(const PairTab &P, const BoysTab &B, int
             const double r = rsqrt(bra.zeta + ket.zeta);
             const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
-            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[7];
             boys_fm<6>(T, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
-            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
             const VT WQx = (VT)(zz * PQx), WQy = (VT)(zz * PQy), WQz = (VT)(zz * PQz);
             const VT oo2z = (VT)bra.oo2z, oo2e = (VT)ket.oo2z, oo2ze = (VT)(0.5 * r2);
@@ -221,108 +221,185 @@ __device__ __forceinline__ void vrr_ffss(const PairTab &P, const BoysTab &B, int
             const VT v54_0_1 = PAz * v33_0_1 + WPz * v33_0_2 + (VT)3.0 * oo2z * (v18_0_1 - rho_z * v18_0_2);
             const VT v55_0_0 = PAz * v34_0_0 + WPz * v34_0_1 + (VT)4.0 * oo2z * (v19_0_0 - rho_z * v19_0_1);
             const VT v55_0_1 = PAz * v34_0_1 + WPz * v34_0_2 + (VT)4.0 * oo2z * (v19_0_1 - rho_z * v19_0_2);
-            const VT v56_0_0 = PAx * v35_0_0 + WPx * v35_0_1 + (VT)5.0 * oo2z * (v20_0_0 - rho_z * v20_0_1);
-            const VT v57_0_0 = PAx * v36_0_0 + WPx * v36_0_1 + (VT)4.0 * oo2z * (v21_0_0 - rho_z * v21_0_1);
-            const VT v58_0_0 = PAx * v37_0_0 + WPx * v37_0_1 + (VT)4.0 * oo2z * (v22_0_0 - rho_z * v22_0_1);
-            const VT v59_0_0 = PAx * v38_0_0 + WPx * v38_0_1 + (VT)3.0 * oo2z * (v23_0_0 - rho_z * v23_0_1);
-            const VT v60_0_0 = PAx * v39_0_0 + WPx * v39_0_1 + (VT)3.0 * oo2z * (v24_0_0 - rho_z * v24_0_1);
-            const VT v61_0_0 = PAx * v40_0_0 + WPx * v40_0_1 + (VT)3.0 * oo2z * (v25_0_0 - rho_z * v25_0_1);
-            const VT v62_0_0 = PAx * v41_0_0 + WPx * v41_0_1 + (VT)2.0 * oo2z * (v26_0_0 - rho_z * v26_0_1);
-            const VT v63_0_0 = PAx * v42_0_0 + WPx * v42_0_1 + (VT)2.0 * oo2z * (v27_0_0 - rho_z * v27_0_1);
-            const VT v64_0_0 = PAx * v43_0_0 + WPx * v43_0_1 + (VT)2.0 * oo2z * (v28_0_0 - rho_z * v28_0_1);
-            const VT v65_0_0 = PAx * v44_0_0 + WPx * v44_0_1 + (VT)2.0 * oo2z * (v29_0_0 - rho_z * v29_0_1);
-            const VT v66_0_0 = PAy * v41_0_0 + WPy * v41_0_1 + (VT)3.0 * oo2z * (v23_0_0 - rho_z * v23_0_1);
-            const VT v67_0_0 = PAy * v42_0_0 + WPy * v42_0_1 + (VT)2.0 * oo2z * (v24_0_0 - rho_z * v24_0_1);
-            const VT v68_0_0 = PAx * v47_0_0 + WPx * v47_0_1 + (VT)1.0 * oo2z * (v32_0_0 - rho_z * v32_0_1);
-            const VT v69_0_0 = PAz * v43_0_0 + WPz * v43_0_1 + (VT)2.0 * oo2z * (v24_0_0 - rho_z * v24_0_1);
-            const VT v70_0_0 = PAz * v44_0_0 + WPz * v44_0_1 + (VT)3.0 * oo2z * (v25_0_0 - rho_z * v25_0_1);
-            const VT v71_0_0 = PAy * v45_0_0 + WPy * v45_0_1 + (VT)4.0 * oo2z * (v26_0_0 - rho_z * v26_0_1);
-            const VT v72_0_0 = PAy * v46_0_0 + WPy * v46_0_1 + (VT)3.0 * oo2z * (v27_0_0 - rho_z * v27_0_1);
-            const VT v73_0_0 = PAy * v47_0_0 + WPy * v47_0_1 + (VT)2.0 * oo2z * (v28_0_0 - rho_z * v28_0_1);
-            const VT v74_0_0 = PAz * v47_0_0 + WPz * v47_0_1 + (VT)2.0 * oo2z * (v27_0_0 - rho_z * v27_0_1);
-            const VT v75_0_0 = PAz * v48_0_0 + WPz * v48_0_1 + (VT)3.0 * oo2z * (v28_0_0 - rho_z * v28_0_1);
-            const VT v76_0_0 = PAz * v49_0_0 + WPz * v49_0_1 + (VT)4.0 * oo2z * (v29_0_0 - rho_z * v29_0_1);
-            const VT v77_0_0 = PAy * v50_0_0 + WPy * v50_0_1 + (VT)5.0 * oo2z * (v30_0_0 - rho_z * v30_0_1);
-            const VT v78_0_0 = PAy * v51_0_0 + WPy * v51_0_1 + (VT)4.0 * oo2z * (v31_0_0 - rho_z * v31_0_1);
-            const VT v79_0_0 = PAy * v52_0_0 + WPy * v52_0_1 + (VT)3.0 * oo2z * (v32_0_0 - rho_z * v32_0_1);
-            const VT v80_0_0 = PAy * v53_0_0 + WPy * v53_0_1 + (VT)2.0 * oo2z * (v33_0_0 - rho_z * v33_0_1);
-            const VT v81_0_0 = PAz * v53_0_0 + WPz * v53_0_1 + (VT)3.0 * oo2z * (v32_0_0 - rho_z * v32_0_1);
-            const VT v82_0_0 = PAz * v54_0_0 + WPz * v54_0_1 + (VT)4.0 * oo2z * (v33_0_0 - rho_z * v33_0_1);
-            const VT v83_0_0 = PAz * v55_0_0 + WPz * v55_0_1 + (VT)5.0 * oo2z * (v34_0_0 - rho_z * v34_0_1);
-            acc[0] += (double)v10_0_0;
-            acc[1] += (double)v11_0_0;
-            acc[2] += (double)v12_0_0;
-            acc[3] += (double)v13_0_0;
-            acc[4] += (double)v14_0_0;
-            acc[5] += (double)v15_0_0;
-            acc[6] += (double)v16_0_0;
-            acc[7] += (double)v17_0_0;
-            acc[8] += (double)v18_0_0;
-            acc[9] += (double)v19_0_0;
-            acc[10] += (double)v20_0_0;
-            acc[11] += (double)v21_0_0;
-            acc[12] += (double)v22_0_0;
-            acc[13] += (double)v23_0_0;
-            acc[14] += (double)v24_0_0;
-            acc[15] += (double)v25_0_0;
-            acc[16] += (double)v26_0_0;
-            acc[17] += (double)v27_0_0;
-            acc[18] += (double)v28_0_0;
-            acc[19] += (double)v29_0_0;
-            acc[20] += (double)v30_0_0;
-            acc[21] += (double)v31_0_0;
-            acc[22] += (double)v32_0_0;
-            acc[23] += (double)v33_0_0;
-            acc[24] += (double)v34_0_0;
-            acc[25] += (double)v35_0_0;
-            acc[26] += (double)v36_0_0;
-            acc[27] += (double)v37_0_0;
-            acc[28] += (double)v38_0_0;
-            acc[29] += (double)v39_0_0;
-            acc[30] += (double)v40_0_0;
-            acc[31] += (double)v41_0_0;
-            acc[32] += (double)v42_0_0;
-            acc[33] += (double)v43_0_0;
-            acc[34] += (double)v44_0_0;
-            acc[35] += (double)v45_0_0;
-            acc[36] += (double)v46_0_0;
-            acc[37] += (double)v47_0_0;
-            acc[38] += (double)v48_0_0;
-            acc[39] += (double)v49_0_0;
-            acc[40] += (double)v50_0_0;
-            acc[41] += (double)v51_0_0;
-            acc[42] += (double)v52_0_0;
-            acc[43] += (double)v53_0_0;
-            acc[44] += (double)v54_0_0;
-            acc[45] += (double)v55_0_0;
-            acc[46] += (double)v56_0_0;
-            acc[47] += (double)v57_0_0;
-            acc[48] += (double)v58_0_0;
-            acc[49] += (double)v59_0_0;
-            acc[50] += (double)v60_0_0;
-            acc[51] += (double)v61_0_0;
-            acc[52] += (double)v62_0_0;
-            acc[53] += (double)v63_0_0;
-            acc[54] += (double)v64_0_0;
-            acc[55] += (double)v65_0_0;
-            acc[56] += (double)v66_0_0;
-            acc[57] += (double)v67_0_0;
-            acc[58] += (double)v68_0_0;
-            acc[59] += (double)v69_0_0;
-            acc[60] += (double)v70_0_0;
-            acc[61] += (double)v71_0_0;
-            acc[62] += (double)v72_0_0;
-            acc[63] += (double)v73_0_0;
-            acc[64] += (double)v74_0_0;
-            acc[65] += (double)v75_0_0;
-            acc[66] += (double)v76_0_0;
-            acc[67] += (double)v77_0_0;
-            acc[68] += (double)v78_0_0;
-            acc[69] += (double)v79_0_0;
-            acc[70] += (double)v80_0_0;
-            acc[71] += (double)v81_0_0;
-            acc[72] += (double)v82_0_0;
-            acc[73] += (double)v83_0_0;
+            if constexpr (sizeof(VT) == 8) {
+                acc[0] += (double)v10_0_0;
+                acc[1] += (double)v11_0_0;
+                acc[2] += (double)v12_0_0;
+                acc[3] += (double)v13_0_0;
+                acc[4] += (double)v14_0_0;
+                acc[5] += (double)v15_0_0;
+                acc[6] += (double)v16_0_0;
+                acc[7] += (double)v17_0_0;
+                acc[8] += (double)v18_0_0;
+                acc[9] += (double)v19_0_0;
+                acc[10] += (double)v20_0_0;
+                acc[11] += (double)v21_0_0;
+                acc[12] += (double)v22_0_0;
+                acc[13] += (double)v23_0_0;
+                acc[14] += (double)v24_0_0;
+                acc[15] += (double)v25_0_0;
+                acc[16] += (double)v26_0_0;
+                acc[17] += (double)v27_0_0;
+                acc[18] += (double)v28_0_0;
+                acc[19] += (double)v29_0_0;
+                acc[20] += (double)v30_0_0;
+                acc[21] += (double)v31_0_0;
+                acc[22] += (double)v32_0_0;
+                acc[23] += (double)v33_0_0;
+                acc[24] += (double)v34_0_0;
+                acc[25] += (double)v35_0_0;
+                acc[26] += (double)v36_0_0;
+                acc[27] += (double)v37_0_0;
+                acc[28] += (double)v38_0_0;
+                acc[29] += (double)v39_0_0;
+                acc[30] += (double)v40_0_0;
+                acc[31] += (double)v41_0_0;
+                acc[32] += (double)v42_0_0;
+                acc[33] += (double)v43_0_0;
+                acc[34] += (double)v44_0_0;
+                acc[35] += (double)v45_0_0;
+                acc[36] += (double)v46_0_0;
+                acc[37] += (double)v47_0_0;
+                acc[38] += (double)v48_0_0;
+                acc[39] += (double)v49_0_0;
+                acc[40] += (double)v50_0_0;
+                acc[41] += (double)v51_0_0;
+                acc[42] += (double)v52_0_0;
+                acc[43] += (double)v53_0_0;
+                acc[44] += (double)v54_0_0;
+                acc[45] += (double)v55_0_0;
+                acc[46] = fma(PAx, v35_0_0, fma(WPx, v35_0_1, fma(5.0 * oo2z, (v20_0_0 - rho_z * v20_0_1), acc[46])));
+                acc[47] = fma(PAx, v36_0_0, fma(WPx, v36_0_1, fma(4.0 * oo2z, (v21_0_0 - rho_z * v21_0_1), acc[47])));
+                acc[48] = fma(PAx, v37_0_0, fma(WPx, v37_0_1, fma(4.0 * oo2z, (v22_0_0 - rho_z * v22_0_1), acc[48])));
+                acc[49] = fma(PAx, v38_0_0, fma(WPx, v38_0_1, fma(3.0 * oo2z, (v23_0_0 - rho_z * v23_0_1), acc[49])));
+                acc[50] = fma(PAx, v39_0_0, fma(WPx, v39_0_1, fma(3.0 * oo2z, (v24_0_0 - rho_z * v24_0_1), acc[50])));
+                acc[51] = fma(PAx, v40_0_0, fma(WPx, v40_0_1, fma(3.0 * oo2z, (v25_0_0 - rho_z * v25_0_1), acc[51])));
+                acc[52] = fma(PAx, v41_0_0, fma(WPx, v41_0_1, fma(2.0 * oo2z, (v26_0_0 - rho_z * v26_0_1), acc[52])));
+                acc[53] = fma(PAx, v42_0_0, fma(WPx, v42_0_1, fma(2.0 * oo2z, (v27_0_0 - rho_z * v27_0_1), acc[53])));
+                acc[54] = fma(PAx, v43_0_0, fma(WPx, v43_0_1, fma(2.0 * oo2z, (v28_0_0 - rho_z * v28_0_1), acc[54])));
+                acc[55] = fma(PAx, v44_0_0, fma(WPx, v44_0_1, fma(2.0 * oo2z, (v29_0_0 - rho_z * v29_0_1), acc[55])));
+                acc[56] = fma(PAy, v41_0_0, fma(WPy, v41_0_1, fma(3.0 * oo2z, (v23_0_0 - rho_z * v23_0_1), acc[56])));
+                acc[57] = fma(PAy, v42_0_0, fma(WPy, v42_0_1, fma(2.0 * oo2z, (v24_0_0 - rho_z * v24_0_1), acc[57])));
+                acc[58] = fma(PAx, v47_0_0, fma(WPx, v47_0_1, fma(1.0 * oo2z, (v32_0_0 - rho_z * v32_0_1), acc[58])));
+                acc[59] = fma(PAz, v43_0_0, fma(WPz, v43_0_1, fma(2.0 * oo2z, (v24_0_0 - rho_z * v24_0_1), acc[59])));
+                acc[60] = fma(PAz, v44_0_0, fma(WPz, v44_0_1, fma(3.0 * oo2z, (v25_0_0 - rho_z * v25_0_1), acc[60])));
+                acc[61] = fma(PAy, v45_0_0, fma(WPy, v45_0_1, fma(4.0 * oo2z, (v26_0_0 - rho_z * v26_0_1), acc[61])));
+                acc[62] = fma(PAy, v46_0_0, fma(WPy, v46_0_1, fma(3.0 * oo2z, (v27_0_0 - rho_z * v27_0_1), acc[62])));
+                acc[63] = fma(PAy, v47_0_0, fma(WPy, v47_0_1, fma(2.0 * oo2z, (v28_0_0 - rho_z * v28_0_1), acc[63])));
+                acc[64] = fma(PAz, v47_0_0, fma(WPz, v47_0_1, fma(2.0 * oo2z, (v27_0_0 - rho_z * v27_0_1), acc[64])));
+                acc[65] = fma(PAz, v48_0_0, fma(WPz, v48_0_1, fma(3.0 * oo2z, (v28_0_0 - rho_z * v28_0_1), acc[65])));
+                acc[66] = fma(PAz, v49_0_0, fma(WPz, v49_0_1, fma(4.0 * oo2z, (v29_0_0 - rho_z * v29_0_1), acc[66])));
+                acc[67] = fma(PAy, v50_0_0, fma(WPy, v50_0_1, fma(5.0 * oo2z, (v30_0_0 - rho_z * v30_0_1), acc[67])));
+                acc[68] = fma(PAy, v51_0_0, fma(WPy, v51_0_1, fma(4.0 * oo2z, (v31_0_0 - rho_z * v31_0_1), acc[68])));
+                acc[69] = fma(PAy, v52_0_0, fma(WPy, v52_0_1, fma(3.0 * oo2z, (v32_0_0 - rho_z * v32_0_1), acc[69])));
+                acc[70] = fma(PAy, v53_0_0, fma(WPy, v53_0_1, fma(2.0 * oo2z, (v33_0_0 - rho_z * v33_0_1), acc[70])));
+                acc[71] = fma(PAz, v53_0_0, fma(WPz, v53_0_1, fma(3.0 * oo2z, (v32_0_0 - rho_z * v32_0_1), acc[71])));
+                acc[72] = fma(PAz, v54_0_0, fma(WPz, v54_0_1, fma(4.0 * oo2z, (v33_0_0 - rho_z * v33_0_1), acc[72])));
+                acc[73] = fma(PAz, v55_0_0, fma(WPz, v55_0_1, fma(5.0 * oo2z, (v34_0_0 - rho_z * v34_0_1), acc[73])));
+            } else {
+                acc[0] += (double)v10_0_0;
+                acc[1] += (double)v11_0_0;
+                acc[2] += (double)v12_0_0;
+                acc[3] += (double)v13_0_0;
+                acc[4] += (double)v14_0_0;
+                acc[5] += (double)v15_0_0;
+                acc[6] += (double)v16_0_0;
+                acc[7] += (double)v17_0_0;
+                acc[8] += (double)v18_0_0;
+                acc[9] += (double)v19_0_0;
+                acc[10] += (double)v20_0_0;
+                acc[11] += (double)v21_0_0;
+                acc[12] += (double)v22_0_0;
+                acc[13] += (double)v23_0_0;
+                acc[14] += (double)v24_0_0;
+                acc[15] += (double)v25_0_0;
+                acc[16] += (double)v26_0_0;
+                acc[17] += (double)v27_0_0;
+                acc[18] += (double)v28_0_0;
+                acc[19] += (double)v29_0_0;
+                acc[20] += (double)v30_0_0;
+                acc[21] += (double)v31_0_0;
+                acc[22] += (double)v32_0_0;
+                acc[23] += (double)v33_0_0;
+                acc[24] += (double)v34_0_0;
+                acc[25] += (double)v35_0_0;
+                acc[26] += (double)v36_0_0;
+                acc[27] += (double)v37_0_0;
+                acc[28] += (double)v38_0_0;
+                acc[29] += (double)v39_0_0;
+                acc[30] += (double)v40_0_0;
+                acc[31] += (double)v41_0_0;
+                acc[32] += (double)v42_0_0;
+                acc[33] += (double)v43_0_0;
+                acc[34] += (double)v44_0_0;
+                acc[35] += (double)v45_0_0;
+                acc[36] += (double)v46_0_0;
+                acc[37] += (double)v47_0_0;
+                acc[38] += (double)v48_0_0;
+                acc[39] += (double)v49_0_0;
+                acc[40] += (double)v50_0_0;
+                acc[41] += (double)v51_0_0;
+                acc[42] += (double)v52_0_0;
+                acc[43] += (double)v53_0_0;
+                acc[44] += (double)v54_0_0;
+                acc[45] += (double)v55_0_0;
+                const VT v56_0_0 = PAx * v35_0_0 + WPx * v35_0_1 + (VT)5.0 * oo2z * (v20_0_0 - rho_z * v20_0_1);
+                acc[46] += (double)v56_0_0;
+                const VT v57_0_0 = PAx * v36_0_0 + WPx * v36_0_1 + (VT)4.0 * oo2z * (v21_0_0 - rho_z * v21_0_1);
+                acc[47] += (double)v57_0_0;
+                const VT v58_0_0 = PAx * v37_0_0 + WPx * v37_0_1 + (VT)4.0 * oo2z * (v22_0_0 - rho_z * v22_0_1);
+                acc[48] += (double)v58_0_0;
+                const VT v59_0_0 = PAx * v38_0_0 + WPx * v38_0_1 + (VT)3.0 * oo2z * (v23_0_0 - rho_z * v23_0_1);
+                acc[49] += (double)v59_0_0;
+                const VT v60_0_0 = PAx * v39_0_0 + WPx * v39_0_1 + (VT)3.0 * oo2z * (v24_0_0 - rho_z * v24_0_1);
+                acc[50] += (double)v60_0_0;
+                const VT v61_0_0 = PAx * v40_0_0 + WPx * v40_0_1 + (VT)3.0 * oo2z * (v25_0_0 - rho_z * v25_0_1);
+                acc[51] += (double)v61_0_0;
+                const VT v62_0_0 = PAx * v41_0_0 + WPx * v41_0_1 + (VT)2.0 * oo2z * (v26_0_0 - rho_z * v26_0_1);
+                acc[52] += (double)v62_0_0;
+                const VT v63_0_0 = PAx * v42_0_0 + WPx * v42_0_1 + (VT)2.0 * oo2z * (v27_0_0 - rho_z * v27_0_1);
+                acc[53] += (double)v63_0_0;
+                const VT v64_0_0 = PAx * v43_0_0 + WPx * v43_0_1 + (VT)2.0 * oo2z * (v28_0_0 - rho_z * v28_0_1);
+                acc[54] += (double)v64_0_0;
+                const VT v65_0_0 = PAx * v44_0_0 + WPx * v44_0_1 + (VT)2.0 * oo2z * (v29_0_0 - rho_z * v29_0_1);
+                acc[55] += (double)v65_0_0;
+                const VT v66_0_0 = PAy * v41_0_0 + WPy * v41_0_1 + (VT)3.0 * oo2z * (v23_0_0 - rho_z * v23_0_1);
+                acc[56] += (double)v66_0_0;
+                const VT v67_0_0 = PAy * v42_0_0 + WPy * v42_0_1 + (VT)2.0 * oo2z * (v24_0_0 - rho_z * v24_0_1);
+                acc[57] += (double)v67_0_0;
+                const VT v68_0_0 = PAx * v47_0_0 + WPx * v47_0_1 + (VT)1.0 * oo2z * (v32_0_0 - rho_z * v32_0_1);
+                acc[58] += (double)v68_0_0;
+                const VT v69_0_0 = PAz * v43_0_0 + WPz * v43_0_1 + (VT)2.0 * oo2z * (v24_0_0 - rho_z * v24_0_1);
+                acc[59] += (double)v69_0_0;
+                const VT v70_0_0 = PAz * v44_0_0 + WPz * v44_0_1 + (VT)3.0 * oo2z * (v25_0_0 - rho_z * v25_0_1);
+                acc[60] += (double)v70_0_0;
+                const VT v71_0_0 = PAy * v45_0_0 + WPy * v45_0_1 + (VT)4.0 * oo2z * (v26_0_0 - rho_z * v26_0_1);
+                acc[61] += (double)v71_0_0;
+                const VT v72_0_0 = PAy * v46_0_0 + WPy * v46_0_1 + (VT)3.0 * oo2z * (v27_0_0 - rho_z * v27_0_1);
+                acc[62] += (double)v72_0_0;
+                const VT v73_0_0 = PAy * v47_0_0 + WPy * v47_0_1 + (VT)2.0 * oo2z * (v28_0_0 - rho_z * v28_0_1);
+                acc[63] += (double)v73_0_0;
+                const VT v74_0_0 = PAz * v47_0_0 + WPz * v47_0_1 + (VT)2.0 * oo2z * (v27_0_0 - rho_z * v27_0_1);
+                acc[64] += (double)v74_0_0;
+                const VT v75_0_0 = PAz * v48_0_0 + WPz * v48_0_1 + (VT)3.0 * oo2z * (v28_0_0 - rho_z * v28_0_1);
+                acc[65] += (double)v75_0_0;
+                const VT v76_0_0 = PAz * v49_0_0 + WPz * v49_0_1 + (VT)4.0 * oo2z * (v29_0_0 - rho_z * v29_0_1);
+                acc[66] += (double)v76_0_0;
+                const VT v77_0_0 = PAy * v50_0_0 + WPy * v50_0_1 + (VT)5.0 * oo2z * (v30_0_0 - rho_z * v30_0_1);
+                acc[67] += (double)v77_0_0;
+                const VT v78_0_0 = PAy * v51_0_0 + WPy * v51_0_1 + (VT)4.0 * oo2z * (v31_0_0 - rho_z * v31_0_1);
+                acc[68] += (double)v78_0_0;
+                const VT v79_0_0 = PAy * v52_0_0 + WPy * v52_0_1 + (VT)3.0 * oo2z * (v32_0_0 - rho_z * v32_0_1);
+                acc[69] += (double)v79_0_0;
+                const VT v80_0_0 = PAy * v53_0_0 + WPy * v53_0_1 + (VT)2.0 * oo2z * (v33_0_0 - rho_z * v33_0_1);
+                acc[70] += (double)v80_0_0;
+                const VT v81_0_0 = PAz * v53_0_0 + WPz * v53_0_1 + (VT)3.0 * oo2z * (v32_0_0 - rho_z * v32_0_1);
+                acc[71] += (double)v81_0_0;
+                const VT v82_0_0 = PAz * v54_0_0 + WPz * v54_0_1 + (VT)4.0 * oo2z * (v33_0_0 - rho_z * v33_0_1);
+                acc[72] += (double)v82_0_0;
+                const VT v83_0_0 = PAz * v55_0_0 + WPz * v55_0_1 + (VT)5.0 * oo2z * (v34_0_0 - rho_z * v34_0_1);
+                acc[73] += (double)v83_0_0;
+            }
         }
     }
 }

@@ -25,13 +25,13 @@ __device__ __forceinline__ void vrr_fppp(const PairTab &P, const BoysTab &B, int
             const double r = rsqrt(bra.zeta + ket.zeta);
             const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
-            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[7];
             boys_fm<6>(T, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
-            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
             const VT WQx = (VT)(zz * PQx), WQy = (VT)(zz * PQy), WQz = (VT)(zz * PQz);
             const VT oo2z = (VT)bra.oo2z, oo2e = (VT)ket.oo2z, oo2ze = (VT)(0.5 * r2);
@@ -347,381 +347,609 @@ __device__ __forceinline__ void vrr_fppp(const PairTab &P, const BoysTab &B, int
             const VT v33_3_1 = QCz * v33_0_1 + WQz * v33_0_2 + (VT)3.0 * oo2ze * v18_0_2;
             const VT v34_3_0 = QCz * v34_0_0 + WQz * v34_0_1 + (VT)4.0 * oo2ze * v19_0_1;
             const VT v34_3_1 = QCz * v34_0_1 + WQz * v34_0_2 + (VT)4.0 * oo2ze * v19_0_2;
-            const VT v10_4_0 = QCx * v10_1_0 + WQx * v10_1_1 + (VT)3.0 * oo2ze * v4_1_1 + (VT)1.0 * oo2e * (v10_0_0 - rho_e * v10_0_1);
-            const VT v11_4_0 = QCx * v11_1_0 + WQx * v11_1_1 + (VT)2.0 * oo2ze * v5_1_1 + (VT)1.0 * oo2e * (v11_0_0 - rho_e * v11_0_1);
-            const VT v12_4_0 = QCx * v12_1_0 + WQx * v12_1_1 + (VT)2.0 * oo2ze * v6_1_1 + (VT)1.0 * oo2e * (v12_0_0 - rho_e * v12_0_1);
-            const VT v13_4_0 = QCx * v13_1_0 + WQx * v13_1_1 + (VT)1.0 * oo2ze * v7_1_1 + (VT)1.0 * oo2e * (v13_0_0 - rho_e * v13_0_1);
-            const VT v14_4_0 = QCx * v14_1_0 + WQx * v14_1_1 + (VT)1.0 * oo2ze * v9_1_1 + (VT)1.0 * oo2e * (v14_0_0 - rho_e * v14_0_1);
-            const VT v15_4_0 = QCx * v15_1_0 + WQx * v15_1_1 + (VT)1.0 * oo2ze * v8_1_1 + (VT)1.0 * oo2e * (v15_0_0 - rho_e * v15_0_1);
-            const VT v16_4_0 = QCx * v16_1_0 + WQx * v16_1_1 + (VT)1.0 * oo2e * (v16_0_0 - rho_e * v16_0_1);
-            const VT v17_4_0 = QCx * v17_1_0 + WQx * v17_1_1 + (VT)1.0 * oo2e * (v17_0_0 - rho_e * v17_0_1);
-            const VT v18_4_0 = QCx * v18_1_0 + WQx * v18_1_1 + (VT)1.0 * oo2e * (v18_0_0 - rho_e * v18_0_1);
-            const VT v19_4_0 = QCx * v19_1_0 + WQx * v19_1_1 + (VT)1.0 * oo2e * (v19_0_0 - rho_e * v19_0_1);
-            const VT v20_4_0 = QCx * v20_1_0 + WQx * v20_1_1 + (VT)4.0 * oo2ze * v10_1_1 + (VT)1.0 * oo2e * (v20_0_0 - rho_e * v20_0_1);
-            const VT v21_4_0 = QCx * v21_1_0 + WQx * v21_1_1 + (VT)3.0 * oo2ze * v11_1_1 + (VT)1.0 * oo2e * (v21_0_0 - rho_e * v21_0_1);
-            const VT v22_4_0 = QCx * v22_1_0 + WQx * v22_1_1 + (VT)3.0 * oo2ze * v12_1_1 + (VT)1.0 * oo2e * (v22_0_0 - rho_e * v22_0_1);
-            const VT v23_4_0 = QCx * v23_1_0 + WQx * v23_1_1 + (VT)2.0 * oo2ze * v13_1_1 + (VT)1.0 * oo2e * (v23_0_0 - rho_e * v23_0_1);
-            const VT v24_4_0 = QCx * v24_1_0 + WQx * v24_1_1 + (VT)2.0 * oo2ze * v15_1_1 + (VT)1.0 * oo2e * (v24_0_0 - rho_e * v24_0_1);
-            const VT v25_4_0 = QCx * v25_1_0 + WQx * v25_1_1 + (VT)2.0 * oo2ze * v14_1_1 + (VT)1.0 * oo2e * (v25_0_0 - rho_e * v25_0_1);
-            const VT v26_4_0 = QCx * v26_1_0 + WQx * v26_1_1 + (VT)1.0 * oo2ze * v16_1_1 + (VT)1.0 * oo2e * (v26_0_0 - rho_e * v26_0_1);
-            const VT v27_4_0 = QCx * v27_1_0 + WQx * v27_1_1 + (VT)1.0 * oo2ze * v17_1_1 + (VT)1.0 * oo2e * (v27_0_0 - rho_e * v27_0_1);
-            const VT v28_4_0 = QCx * v28_1_0 + WQx * v28_1_1 + (VT)1.0 * oo2ze * v18_1_1 + (VT)1.0 * oo2e * (v28_0_0 - rho_e * v28_0_1);
-            const VT v29_4_0 = QCx * v29_1_0 + WQx * v29_1_1 + (VT)1.0 * oo2ze * v19_1_1 + (VT)1.0 * oo2e * (v29_0_0 - rho_e * v29_0_1);
-            const VT v30_4_0 = QCx * v30_1_0 + WQx * v30_1_1 + (VT)1.0 * oo2e * (v30_0_0 - rho_e * v30_0_1);
-            const VT v31_4_0 = QCx * v31_1_0 + WQx * v31_1_1 + (VT)1.0 * oo2e * (v31_0_0 - rho_e * v31_0_1);
-            const VT v32_4_0 = QCx * v32_1_0 + WQx * v32_1_1 + (VT)1.0 * oo2e * (v32_0_0 - rho_e * v32_0_1);
-            const VT v33_4_0 = QCx * v33_1_0 + WQx * v33_1_1 + (VT)1.0 * oo2e * (v33_0_0 - rho_e * v33_0_1);
-            const VT v34_4_0 = QCx * v34_1_0 + WQx * v34_1_1 + (VT)1.0 * oo2e * (v34_0_0 - rho_e * v34_0_1);
-            const VT v10_5_0 = QCx * v10_2_0 + WQx * v10_2_1 + (VT)3.0 * oo2ze * v4_2_1;
-            const VT v11_5_0 = QCx * v11_2_0 + WQx * v11_2_1 + (VT)2.0 * oo2ze * v5_2_1;
-            const VT v12_5_0 = QCx * v12_2_0 + WQx * v12_2_1 + (VT)2.0 * oo2ze * v6_2_1;
-            const VT v13_5_0 = QCx * v13_2_0 + WQx * v13_2_1 + (VT)1.0 * oo2ze * v7_2_1;
-            const VT v14_5_0 = QCx * v14_2_0 + WQx * v14_2_1 + (VT)1.0 * oo2ze * v9_2_1;
-            const VT v15_5_0 = QCx * v15_2_0 + WQx * v15_2_1 + (VT)1.0 * oo2ze * v8_2_1;
-            const VT v16_5_0 = QCx * v16_2_0 + WQx * v16_2_1;
-            const VT v17_5_0 = QCx * v17_2_0 + WQx * v17_2_1;
-            const VT v18_5_0 = QCx * v18_2_0 + WQx * v18_2_1;
-            const VT v19_5_0 = QCx * v19_2_0 + WQx * v19_2_1;
-            const VT v20_5_0 = QCx * v20_2_0 + WQx * v20_2_1 + (VT)4.0 * oo2ze * v10_2_1;
-            const VT v21_5_0 = QCx * v21_2_0 + WQx * v21_2_1 + (VT)3.0 * oo2ze * v11_2_1;
-            const VT v22_5_0 = QCx * v22_2_0 + WQx * v22_2_1 + (VT)3.0 * oo2ze * v12_2_1;
-            const VT v23_5_0 = QCx * v23_2_0 + WQx * v23_2_1 + (VT)2.0 * oo2ze * v13_2_1;
-            const VT v24_5_0 = QCx * v24_2_0 + WQx * v24_2_1 + (VT)2.0 * oo2ze * v15_2_1;
-            const VT v25_5_0 = QCx * v25_2_0 + WQx * v25_2_1 + (VT)2.0 * oo2ze * v14_2_1;
-            const VT v26_5_0 = QCx * v26_2_0 + WQx * v26_2_1 + (VT)1.0 * oo2ze * v16_2_1;
-            const VT v27_5_0 = QCx * v27_2_0 + WQx * v27_2_1 + (VT)1.0 * oo2ze * v17_2_1;
-            const VT v28_5_0 = QCx * v28_2_0 + WQx * v28_2_1 + (VT)1.0 * oo2ze * v18_2_1;
-            const VT v29_5_0 = QCx * v29_2_0 + WQx * v29_2_1 + (VT)1.0 * oo2ze * v19_2_1;
-            const VT v30_5_0 = QCx * v30_2_0 + WQx * v30_2_1;
-            const VT v31_5_0 = QCx * v31_2_0 + WQx * v31_2_1;
-            const VT v32_5_0 = QCx * v32_2_0 + WQx * v32_2_1;
-            const VT v33_5_0 = QCx * v33_2_0 + WQx * v33_2_1;
-            const VT v34_5_0 = QCx * v34_2_0 + WQx * v34_2_1;
-            const VT v10_6_0 = QCx * v10_3_0 + WQx * v10_3_1 + (VT)3.0 * oo2ze * v4_3_1;
-            const VT v11_6_0 = QCx * v11_3_0 + WQx * v11_3_1 + (VT)2.0 * oo2ze * v5_3_1;
-            const VT v12_6_0 = QCx * v12_3_0 + WQx * v12_3_1 + (VT)2.0 * oo2ze * v6_3_1;
-            const VT v13_6_0 = QCx * v13_3_0 + WQx * v13_3_1 + (VT)1.0 * oo2ze * v7_3_1;
-            const VT v14_6_0 = QCx * v14_3_0 + WQx * v14_3_1 + (VT)1.0 * oo2ze * v9_3_1;
-            const VT v15_6_0 = QCx * v15_3_0 + WQx * v15_3_1 + (VT)1.0 * oo2ze * v8_3_1;
-            const VT v16_6_0 = QCx * v16_3_0 + WQx * v16_3_1;
-            const VT v17_6_0 = QCx * v17_3_0 + WQx * v17_3_1;
-            const VT v18_6_0 = QCx * v18_3_0 + WQx * v18_3_1;
-            const VT v19_6_0 = QCx * v19_3_0 + WQx * v19_3_1;
-            const VT v20_6_0 = QCx * v20_3_0 + WQx * v20_3_1 + (VT)4.0 * oo2ze * v10_3_1;
-            const VT v21_6_0 = QCx * v21_3_0 + WQx * v21_3_1 + (VT)3.0 * oo2ze * v11_3_1;
-            const VT v22_6_0 = QCx * v22_3_0 + WQx * v22_3_1 + (VT)3.0 * oo2ze * v12_3_1;
-            const VT v23_6_0 = QCx * v23_3_0 + WQx * v23_3_1 + (VT)2.0 * oo2ze * v13_3_1;
-            const VT v24_6_0 = QCx * v24_3_0 + WQx * v24_3_1 + (VT)2.0 * oo2ze * v15_3_1;
-            const VT v25_6_0 = QCx * v25_3_0 + WQx * v25_3_1 + (VT)2.0 * oo2ze * v14_3_1;
-            const VT v26_6_0 = QCx * v26_3_0 + WQx * v26_3_1 + (VT)1.0 * oo2ze * v16_3_1;
-            const VT v27_6_0 = QCx * v27_3_0 + WQx * v27_3_1 + (VT)1.0 * oo2ze * v17_3_1;
-            const VT v28_6_0 = QCx * v28_3_0 + WQx * v28_3_1 + (VT)1.0 * oo2ze * v18_3_1;
-            const VT v29_6_0 = QCx * v29_3_0 + WQx * v29_3_1 + (VT)1.0 * oo2ze * v19_3_1;
-            const VT v30_6_0 = QCx * v30_3_0 + WQx * v30_3_1;
-            const VT v31_6_0 = QCx * v31_3_0 + WQx * v31_3_1;
-            const VT v32_6_0 = QCx * v32_3_0 + WQx * v32_3_1;
-            const VT v33_6_0 = QCx * v33_3_0 + WQx * v33_3_1;
-            const VT v34_6_0 = QCx * v34_3_0 + WQx * v34_3_1;
-            const VT v10_7_0 = QCy * v10_2_0 + WQy * v10_2_1 + (VT)1.0 * oo2e * (v10_0_0 - rho_e * v10_0_1);
-            const VT v11_7_0 = QCy * v11_2_0 + WQy * v11_2_1 + (VT)1.0 * oo2ze * v4_2_1 + (VT)1.0 * oo2e * (v11_0_0 - rho_e * v11_0_1);
-            const VT v12_7_0 = QCy * v12_2_0 + WQy * v12_2_1 + (VT)1.0 * oo2e * (v12_0_0 - rho_e * v12_0_1);
-            const VT v13_7_0 = QCy * v13_2_0 + WQy * v13_2_1 + (VT)2.0 * oo2ze * v5_2_1 + (VT)1.0 * oo2e * (v13_0_0 - rho_e * v13_0_1);
-            const VT v14_7_0 = QCy * v14_2_0 + WQy * v14_2_1 + (VT)1.0 * oo2e * (v14_0_0 - rho_e * v14_0_1);
-            const VT v15_7_0 = QCy * v15_2_0 + WQy * v15_2_1 + (VT)1.0 * oo2ze * v6_2_1 + (VT)1.0 * oo2e * (v15_0_0 - rho_e * v15_0_1);
-            const VT v16_7_0 = QCy * v16_2_0 + WQy * v16_2_1 + (VT)3.0 * oo2ze * v7_2_1 + (VT)1.0 * oo2e * (v16_0_0 - rho_e * v16_0_1);
-            const VT v17_7_0 = QCy * v17_2_0 + WQy * v17_2_1 + (VT)2.0 * oo2ze * v8_2_1 + (VT)1.0 * oo2e * (v17_0_0 - rho_e * v17_0_1);
-            const VT v18_7_0 = QCy * v18_2_0 + WQy * v18_2_1 + (VT)1.0 * oo2ze * v9_2_1 + (VT)1.0 * oo2e * (v18_0_0 - rho_e * v18_0_1);
-            const VT v19_7_0 = QCy * v19_2_0 + WQy * v19_2_1 + (VT)1.0 * oo2e * (v19_0_0 - rho_e * v19_0_1);
-            const VT v20_7_0 = QCy * v20_2_0 + WQy * v20_2_1 + (VT)1.0 * oo2e * (v20_0_0 - rho_e * v20_0_1);
-            const VT v21_7_0 = QCy * v21_2_0 + WQy * v21_2_1 + (VT)1.0 * oo2ze * v10_2_1 + (VT)1.0 * oo2e * (v21_0_0 - rho_e * v21_0_1);
-            const VT v22_7_0 = QCy * v22_2_0 + WQy * v22_2_1 + (VT)1.0 * oo2e * (v22_0_0 - rho_e * v22_0_1);
-            const VT v23_7_0 = QCy * v23_2_0 + WQy * v23_2_1 + (VT)2.0 * oo2ze * v11_2_1 + (VT)1.0 * oo2e * (v23_0_0 - rho_e * v23_0_1);
-            const VT v24_7_0 = QCy * v24_2_0 + WQy * v24_2_1 + (VT)1.0 * oo2ze * v12_2_1 + (VT)1.0 * oo2e * (v24_0_0 - rho_e * v24_0_1);
-            const VT v25_7_0 = QCy * v25_2_0 + WQy * v25_2_1 + (VT)1.0 * oo2e * (v25_0_0 - rho_e * v25_0_1);
-            const VT v26_7_0 = QCy * v26_2_0 + WQy * v26_2_1 + (VT)3.0 * oo2ze * v13_2_1 + (VT)1.0 * oo2e * (v26_0_0 - rho_e * v26_0_1);
-            const VT v27_7_0 = QCy * v27_2_0 + WQy * v27_2_1 + (VT)2.0 * oo2ze * v15_2_1 + (VT)1.0 * oo2e * (v27_0_0 - rho_e * v27_0_1);
-            const VT v28_7_0 = QCy * v28_2_0 + WQy * v28_2_1 + (VT)1.0 * oo2ze * v14_2_1 + (VT)1.0 * oo2e * (v28_0_0 - rho_e * v28_0_1);
-            const VT v29_7_0 = QCy * v29_2_0 + WQy * v29_2_1 + (VT)1.0 * oo2e * (v29_0_0 - rho_e * v29_0_1);
-            const VT v30_7_0 = QCy * v30_2_0 + WQy * v30_2_1 + (VT)4.0 * oo2ze * v16_2_1 + (VT)1.0 * oo2e * (v30_0_0 - rho_e * v30_0_1);
-            const VT v31_7_0 = QCy * v31_2_0 + WQy * v31_2_1 + (VT)3.0 * oo2ze * v17_2_1 + (VT)1.0 * oo2e * (v31_0_0 - rho_e * v31_0_1);
-            const VT v32_7_0 = QCy * v32_2_0 + WQy * v32_2_1 + (VT)2.0 * oo2ze * v18_2_1 + (VT)1.0 * oo2e * (v32_0_0 - rho_e * v32_0_1);
-            const VT v33_7_0 = QCy * v33_2_0 + WQy * v33_2_1 + (VT)1.0 * oo2ze * v19_2_1 + (VT)1.0 * oo2e * (v33_0_0 - rho_e * v33_0_1);
-            const VT v34_7_0 = QCy * v34_2_0 + WQy * v34_2_1 + (VT)1.0 * oo2e * (v34_0_0 - rho_e * v34_0_1);
-            const VT v10_8_0 = QCy * v10_3_0 + WQy * v10_3_1;
-            const VT v11_8_0 = QCy * v11_3_0 + WQy * v11_3_1 + (VT)1.0 * oo2ze * v4_3_1;
-            const VT v12_8_0 = QCy * v12_3_0 + WQy * v12_3_1;
-            const VT v13_8_0 = QCy * v13_3_0 + WQy * v13_3_1 + (VT)2.0 * oo2ze * v5_3_1;
-            const VT v14_8_0 = QCy * v14_3_0 + WQy * v14_3_1;
-            const VT v15_8_0 = QCy * v15_3_0 + WQy * v15_3_1 + (VT)1.0 * oo2ze * v6_3_1;
-            const VT v16_8_0 = QCy * v16_3_0 + WQy * v16_3_1 + (VT)3.0 * oo2ze * v7_3_1;
-            const VT v17_8_0 = QCy * v17_3_0 + WQy * v17_3_1 + (VT)2.0 * oo2ze * v8_3_1;
-            const VT v18_8_0 = QCy * v18_3_0 + WQy * v18_3_1 + (VT)1.0 * oo2ze * v9_3_1;
-            const VT v19_8_0 = QCy * v19_3_0 + WQy * v19_3_1;
-            const VT v20_8_0 = QCy * v20_3_0 + WQy * v20_3_1;
-            const VT v21_8_0 = QCy * v21_3_0 + WQy * v21_3_1 + (VT)1.0 * oo2ze * v10_3_1;
-            const VT v22_8_0 = QCy * v22_3_0 + WQy * v22_3_1;
-            const VT v23_8_0 = QCy * v23_3_0 + WQy * v23_3_1 + (VT)2.0 * oo2ze * v11_3_1;
-            const VT v24_8_0 = QCy * v24_3_0 + WQy * v24_3_1 + (VT)1.0 * oo2ze * v12_3_1;
-            const VT v25_8_0 = QCy * v25_3_0 + WQy * v25_3_1;
-            const VT v26_8_0 = QCy * v26_3_0 + WQy * v26_3_1 + (VT)3.0 * oo2ze * v13_3_1;
-            const VT v27_8_0 = QCy * v27_3_0 + WQy * v27_3_1 + (VT)2.0 * oo2ze * v15_3_1;
-            const VT v28_8_0 = QCy * v28_3_0 + WQy * v28_3_1 + (VT)1.0 * oo2ze * v14_3_1;
-            const VT v29_8_0 = QCy * v29_3_0 + WQy * v29_3_1;
-            const VT v30_8_0 = QCy * v30_3_0 + WQy * v30_3_1 + (VT)4.0 * oo2ze * v16_3_1;
-            const VT v31_8_0 = QCy * v31_3_0 + WQy * v31_3_1 + (VT)3.0 * oo2ze * v17_3_1;
-            const VT v32_8_0 = QCy * v32_3_0 + WQy * v32_3_1 + (VT)2.0 * oo2ze * v18_3_1;
-            const VT v33_8_0 = QCy * v33_3_0 + WQy * v33_3_1 + (VT)1.0 * oo2ze * v19_3_1;
-            const VT v34_8_0 = QCy * v34_3_0 + WQy * v34_3_1;
-            const VT v10_9_0 = QCz * v10_3_0 + WQz * v10_3_1 + (VT)1.0 * oo2e * (v10_0_0 - rho_e * v10_0_1);
-            const VT v11_9_0 = QCz * v11_3_0 + WQz * v11_3_1 + (VT)1.0 * oo2e * (v11_0_0 - rho_e * v11_0_1);
-            const VT v12_9_0 = QCz * v12_3_0 + WQz * v12_3_1 + (VT)1.0 * oo2ze * v4_3_1 + (VT)1.0 * oo2e * (v12_0_0 - rho_e * v12_0_1);
-            const VT v13_9_0 = QCz * v13_3_0 + WQz * v13_3_1 + (VT)1.0 * oo2e * (v13_0_0 - rho_e * v13_0_1);
-            const VT v14_9_0 = QCz * v14_3_0 + WQz * v14_3_1 + (VT)2.0 * oo2ze * v6_3_1 + (VT)1.0 * oo2e * (v14_0_0 - rho_e * v14_0_1);
-            const VT v15_9_0 = QCz * v15_3_0 + WQz * v15_3_1 + (VT)1.0 * oo2ze * v5_3_1 + (VT)1.0 * oo2e * (v15_0_0 - rho_e * v15_0_1);
-            const VT v16_9_0 = QCz * v16_3_0 + WQz * v16_3_1 + (VT)1.0 * oo2e * (v16_0_0 - rho_e * v16_0_1);
-            const VT v17_9_0 = QCz * v17_3_0 + WQz * v17_3_1 + (VT)1.0 * oo2ze * v7_3_1 + (VT)1.0 * oo2e * (v17_0_0 - rho_e * v17_0_1);
-            const VT v18_9_0 = QCz * v18_3_0 + WQz * v18_3_1 + (VT)2.0 * oo2ze * v8_3_1 + (VT)1.0 * oo2e * (v18_0_0 - rho_e * v18_0_1);
-            const VT v19_9_0 = QCz * v19_3_0 + WQz * v19_3_1 + (VT)3.0 * oo2ze * v9_3_1 + (VT)1.0 * oo2e * (v19_0_0 - rho_e * v19_0_1);
-            const VT v20_9_0 = QCz * v20_3_0 + WQz * v20_3_1 + (VT)1.0 * oo2e * (v20_0_0 - rho_e * v20_0_1);
-            const VT v21_9_0 = QCz * v21_3_0 + WQz * v21_3_1 + (VT)1.0 * oo2e * (v21_0_0 - rho_e * v21_0_1);
-            const VT v22_9_0 = QCz * v22_3_0 + WQz * v22_3_1 + (VT)1.0 * oo2ze * v10_3_1 + (VT)1.0 * oo2e * (v22_0_0 - rho_e * v22_0_1);
-            const VT v23_9_0 = QCz * v23_3_0 + WQz * v23_3_1 + (VT)1.0 * oo2e * (v23_0_0 - rho_e * v23_0_1);
-            const VT v24_9_0 = QCz * v24_3_0 + WQz * v24_3_1 + (VT)1.0 * oo2ze * v11_3_1 + (VT)1.0 * oo2e * (v24_0_0 - rho_e * v24_0_1);
-            const VT v25_9_0 = QCz * v25_3_0 + WQz * v25_3_1 + (VT)2.0 * oo2ze * v12_3_1 + (VT)1.0 * oo2e * (v25_0_0 - rho_e * v25_0_1);
-            const VT v26_9_0 = QCz * v26_3_0 + WQz * v26_3_1 + (VT)1.0 * oo2e * (v26_0_0 - rho_e * v26_0_1);
-            const VT v27_9_0 = QCz * v27_3_0 + WQz * v27_3_1 + (VT)1.0 * oo2ze * v13_3_1 + (VT)1.0 * oo2e * (v27_0_0 - rho_e * v27_0_1);
-            const VT v28_9_0 = QCz * v28_3_0 + WQz * v28_3_1 + (VT)2.0 * oo2ze * v15_3_1 + (VT)1.0 * oo2e * (v28_0_0 - rho_e * v28_0_1);
-            const VT v29_9_0 = QCz * v29_3_0 + WQz * v29_3_1 + (VT)3.0 * oo2ze * v14_3_1 + (VT)1.0 * oo2e * (v29_0_0 - rho_e * v29_0_1);
-            const VT v30_9_0 = QCz * v30_3_0 + WQz * v30_3_1 + (VT)1.0 * oo2e * (v30_0_0 - rho_e * v30_0_1);
-            const VT v31_9_0 = QCz * v31_3_0 + WQz * v31_3_1 + (VT)1.0 * oo2ze * v16_3_1 + (VT)1.0 * oo2e * (v31_0_0 - rho_e * v31_0_1);
-            const VT v32_9_0 = QCz * v32_3_0 + WQz * v32_3_1 + (VT)2.0 * oo2ze * v17_3_1 + (VT)1.0 * oo2e * (v32_0_0 - rho_e * v32_0_1);
-            const VT v33_9_0 = QCz * v33_3_0 + WQz * v33_3_1 + (VT)3.0 * oo2ze * v18_3_1 + (VT)1.0 * oo2e * (v33_0_0 - rho_e * v33_0_1);
-            const VT v34_9_0 = QCz * v34_3_0 + WQz * v34_3_1 + (VT)4.0 * oo2ze * v19_3_1 + (VT)1.0 * oo2e * (v34_0_0 - rho_e * v34_0_1);
-            acc[0] += (double)v10_1_0;
-            acc[1] += (double)v10_2_0;
-            acc[2] += (double)v10_3_0;
-            acc[3] += (double)v10_4_0;
-            acc[4] += (double)v10_5_0;
-            acc[5] += (double)v10_6_0;
-            acc[6] += (double)v10_7_0;
-            acc[7] += (double)v10_8_0;
-            acc[8] += (double)v10_9_0;
-            acc[9] += (double)v11_1_0;
-            acc[10] += (double)v11_2_0;
-            acc[11] += (double)v11_3_0;
-            acc[12] += (double)v11_4_0;
-            acc[13] += (double)v11_5_0;
-            acc[14] += (double)v11_6_0;
-            acc[15] += (double)v11_7_0;
-            acc[16] += (double)v11_8_0;
-            acc[17] += (double)v11_9_0;
-            acc[18] += (double)v12_1_0;
-            acc[19] += (double)v12_2_0;
-            acc[20] += (double)v12_3_0;
-            acc[21] += (double)v12_4_0;
-            acc[22] += (double)v12_5_0;
-            acc[23] += (double)v12_6_0;
-            acc[24] += (double)v12_7_0;
-            acc[25] += (double)v12_8_0;
-            acc[26] += (double)v12_9_0;
-            acc[27] += (double)v13_1_0;
-            acc[28] += (double)v13_2_0;
-            acc[29] += (double)v13_3_0;
-            acc[30] += (double)v13_4_0;
-            acc[31] += (double)v13_5_0;
-            acc[32] += (double)v13_6_0;
-            acc[33] += (double)v13_7_0;
-            acc[34] += (double)v13_8_0;
-            acc[35] += (double)v13_9_0;
-            acc[36] += (double)v14_1_0;
-            acc[37] += (double)v14_2_0;
-            acc[38] += (double)v14_3_0;
-            acc[39] += (double)v14_4_0;
-            acc[40] += (double)v14_5_0;
-            acc[41] += (double)v14_6_0;
-            acc[42] += (double)v14_7_0;
-            acc[43] += (double)v14_8_0;
-            acc[44] += (double)v14_9_0;
-            acc[45] += (double)v15_1_0;
-            acc[46] += (double)v15_2_0;
-            acc[47] += (double)v15_3_0;
-            acc[48] += (double)v15_4_0;
-            acc[49] += (double)v15_5_0;
-            acc[50] += (double)v15_6_0;
-            acc[51] += (double)v15_7_0;
-            acc[52] += (double)v15_8_0;
-            acc[53] += (double)v15_9_0;
-            acc[54] += (double)v16_1_0;
-            acc[55] += (double)v16_2_0;
-            acc[56] += (double)v16_3_0;
-            acc[57] += (double)v16_4_0;
-            acc[58] += (double)v16_5_0;
-            acc[59] += (double)v16_6_0;
-            acc[60] += (double)v16_7_0;
-            acc[61] += (double)v16_8_0;
-            acc[62] += (double)v16_9_0;
-            acc[63] += (double)v17_1_0;
-            acc[64] += (double)v17_2_0;
-            acc[65] += (double)v17_3_0;
-            acc[66] += (double)v17_4_0;
-            acc[67] += (double)v17_5_0;
-            acc[68] += (double)v17_6_0;
-            acc[69] += (double)v17_7_0;
-            acc[70] += (double)v17_8_0;
-            acc[71] += (double)v17_9_0;
-            acc[72] += (double)v18_1_0;
-            acc[73] += (double)v18_2_0;
-            acc[74] += (double)v18_3_0;
-            acc[75] += (double)v18_4_0;
-            acc[76] += (double)v18_5_0;
-            acc[77] += (double)v18_6_0;
-            acc[78] += (double)v18_7_0;
-            acc[79] += (double)v18_8_0;
-            acc[80] += (double)v18_9_0;
-            acc[81] += (double)v19_1_0;
-            acc[82] += (double)v19_2_0;
-            acc[83] += (double)v19_3_0;
-            acc[84] += (double)v19_4_0;
-            acc[85] += (double)v19_5_0;
-            acc[86] += (double)v19_6_0;
-            acc[87] += (double)v19_7_0;
-            acc[88] += (double)v19_8_0;
-            acc[89] += (double)v19_9_0;
-            acc[90] += (double)v20_1_0;
-            acc[91] += (double)v20_2_0;
-            acc[92] += (double)v20_3_0;
-            acc[93] += (double)v20_4_0;
-            acc[94] += (double)v20_5_0;
-            acc[95] += (double)v20_6_0;
-            acc[96] += (double)v20_7_0;
-            acc[97] += (double)v20_8_0;
-            acc[98] += (double)v20_9_0;
-            acc[99] += (double)v21_1_0;
-            acc[100] += (double)v21_2_0;
-            acc[101] += (double)v21_3_0;
-            acc[102] += (double)v21_4_0;
-            acc[103] += (double)v21_5_0;
-            acc[104] += (double)v21_6_0;
-            acc[105] += (double)v21_7_0;
-            acc[106] += (double)v21_8_0;
-            acc[107] += (double)v21_9_0;
-            acc[108] += (double)v22_1_0;
-            acc[109] += (double)v22_2_0;
-            acc[110] += (double)v22_3_0;
-            acc[111] += (double)v22_4_0;
-            acc[112] += (double)v22_5_0;
-            acc[113] += (double)v22_6_0;
-            acc[114] += (double)v22_7_0;
-            acc[115] += (double)v22_8_0;
-            acc[116] += (double)v22_9_0;
-            acc[117] += (double)v23_1_0;
-            acc[118] += (double)v23_2_0;
-            acc[119] += (double)v23_3_0;
-            acc[120] += (double)v23_4_0;
-            acc[121] += (double)v23_5_0;
-            acc[122] += (double)v23_6_0;
-            acc[123] += (double)v23_7_0;
-            acc[124] += (double)v23_8_0;
-            acc[125] += (double)v23_9_0;
-            acc[126] += (double)v24_1_0;
-            acc[127] += (double)v24_2_0;
-            acc[128] += (double)v24_3_0;
-            acc[129] += (double)v24_4_0;
-            acc[130] += (double)v24_5_0;
-            acc[131] += (double)v24_6_0;
-            acc[132] += (double)v24_7_0;
-            acc[133] += (double)v24_8_0;
-            acc[134] += (double)v24_9_0;
-            acc[135] += (double)v25_1_0;
-            acc[136] += (double)v25_2_0;
-            acc[137] += (double)v25_3_0;
-            acc[138] += (double)v25_4_0;
-            acc[139] += (double)v25_5_0;
-            acc[140] += (double)v25_6_0;
-            acc[141] += (double)v25_7_0;
-            acc[142] += (double)v25_8_0;
-            acc[143] += (double)v25_9_0;
-            acc[144] += (double)v26_1_0;
-            acc[145] += (double)v26_2_0;
-            acc[146] += (double)v26_3_0;
-            acc[147] += (double)v26_4_0;
-            acc[148] += (double)v26_5_0;
-            acc[149] += (double)v26_6_0;
-            acc[150] += (double)v26_7_0;
-            acc[151] += (double)v26_8_0;
-            acc[152] += (double)v26_9_0;
-            acc[153] += (double)v27_1_0;
-            acc[154] += (double)v27_2_0;
-            acc[155] += (double)v27_3_0;
-            acc[156] += (double)v27_4_0;
-            acc[157] += (double)v27_5_0;
-            acc[158] += (double)v27_6_0;
-            acc[159] += (double)v27_7_0;
-            acc[160] += (double)v27_8_0;
-            acc[161] += (double)v27_9_0;
-            acc[162] += (double)v28_1_0;
-            acc[163] += (double)v28_2_0;
-            acc[164] += (double)v28_3_0;
-            acc[165] += (double)v28_4_0;
-            acc[166] += (double)v28_5_0;
-            acc[167] += (double)v28_6_0;
-            acc[168] += (double)v28_7_0;
-            acc[169] += (double)v28_8_0;
-            acc[170] += (double)v28_9_0;
-            acc[171] += (double)v29_1_0;
-            acc[172] += (double)v29_2_0;
-            acc[173] += (double)v29_3_0;
-            acc[174] += (double)v29_4_0;
-            acc[175] += (double)v29_5_0;
-            acc[176] += (double)v29_6_0;
-            acc[177] += (double)v29_7_0;
-            acc[178] += (double)v29_8_0;
-            acc[179] += (double)v29_9_0;
-            acc[180] += (double)v30_1_0;
-            acc[181] += (double)v30_2_0;
-            acc[182] += (double)v30_3_0;
-            acc[183] += (double)v30_4_0;
-            acc[184] += (double)v30_5_0;
-            acc[185] += (double)v30_6_0;
-            acc[186] += (double)v30_7_0;
-            acc[187] += (double)v30_8_0;
-            acc[188] += (double)v30_9_0;
-            acc[189] += (double)v31_1_0;
-            acc[190] += (double)v31_2_0;
-            acc[191] += (double)v31_3_0;
-            acc[192] += (double)v31_4_0;
-            acc[193] += (double)v31_5_0;
-            acc[194] += (double)v31_6_0;
-            acc[195] += (double)v31_7_0;
-            acc[196] += (double)v31_8_0;
-            acc[197] += (double)v31_9_0;
-            acc[198] += (double)v32_1_0;
-            acc[199] += (double)v32_2_0;
-            acc[200] += (double)v32_3_0;
-            acc[201] += (double)v32_4_0;
-            acc[202] += (double)v32_5_0;
-            acc[203] += (double)v32_6_0;
-            acc[204] += (double)v32_7_0;
-            acc[205] += (double)v32_8_0;
-            acc[206] += (double)v32_9_0;
-            acc[207] += (double)v33_1_0;
-            acc[208] += (double)v33_2_0;
-            acc[209] += (double)v33_3_0;
-            acc[210] += (double)v33_4_0;
-            acc[211] += (double)v33_5_0;
-            acc[212] += (double)v33_6_0;
-            acc[213] += (double)v33_7_0;
-            acc[214] += (double)v33_8_0;
-            acc[215] += (double)v33_9_0;
-            acc[216] += (double)v34_1_0;
-            acc[217] += (double)v34_2_0;
-            acc[218] += (double)v34_3_0;
-            acc[219] += (double)v34_4_0;
-            acc[220] += (double)v34_5_0;
-            acc[221] += (double)v34_6_0;
-            acc[222] += (double)v34_7_0;
-            acc[223] += (double)v34_8_0;
-            acc[224] += (double)v34_9_0;
+            if constexpr (sizeof(VT) == 8) {
+                acc[0] += (double)v10_1_0;
+                acc[1] += (double)v10_2_0;
+                acc[2] += (double)v10_3_0;
+                acc[3] = fma(QCx, v10_1_0, fma(WQx, v10_1_1, fma(3.0 * oo2ze, v4_1_1, fma(1.0 * oo2e, (v10_0_0 - rho_e * v10_0_1), acc[3]))));
+                acc[4] = fma(QCx, v10_2_0, fma(WQx, v10_2_1, fma(3.0 * oo2ze, v4_2_1, acc[4])));
+                acc[5] = fma(QCx, v10_3_0, fma(WQx, v10_3_1, fma(3.0 * oo2ze, v4_3_1, acc[5])));
+                acc[6] = fma(QCy, v10_2_0, fma(WQy, v10_2_1, fma(1.0 * oo2e, (v10_0_0 - rho_e * v10_0_1), acc[6])));
+                acc[7] = fma(QCy, v10_3_0, fma(WQy, v10_3_1, acc[7]));
+                acc[8] = fma(QCz, v10_3_0, fma(WQz, v10_3_1, fma(1.0 * oo2e, (v10_0_0 - rho_e * v10_0_1), acc[8])));
+                acc[9] += (double)v11_1_0;
+                acc[10] += (double)v11_2_0;
+                acc[11] += (double)v11_3_0;
+                acc[12] = fma(QCx, v11_1_0, fma(WQx, v11_1_1, fma(2.0 * oo2ze, v5_1_1, fma(1.0 * oo2e, (v11_0_0 - rho_e * v11_0_1), acc[12]))));
+                acc[13] = fma(QCx, v11_2_0, fma(WQx, v11_2_1, fma(2.0 * oo2ze, v5_2_1, acc[13])));
+                acc[14] = fma(QCx, v11_3_0, fma(WQx, v11_3_1, fma(2.0 * oo2ze, v5_3_1, acc[14])));
+                acc[15] = fma(QCy, v11_2_0, fma(WQy, v11_2_1, fma(1.0 * oo2ze, v4_2_1, fma(1.0 * oo2e, (v11_0_0 - rho_e * v11_0_1), acc[15]))));
+                acc[16] = fma(QCy, v11_3_0, fma(WQy, v11_3_1, fma(1.0 * oo2ze, v4_3_1, acc[16])));
+                acc[17] = fma(QCz, v11_3_0, fma(WQz, v11_3_1, fma(1.0 * oo2e, (v11_0_0 - rho_e * v11_0_1), acc[17])));
+                acc[18] += (double)v12_1_0;
+                acc[19] += (double)v12_2_0;
+                acc[20] += (double)v12_3_0;
+                acc[21] = fma(QCx, v12_1_0, fma(WQx, v12_1_1, fma(2.0 * oo2ze, v6_1_1, fma(1.0 * oo2e, (v12_0_0 - rho_e * v12_0_1), acc[21]))));
+                acc[22] = fma(QCx, v12_2_0, fma(WQx, v12_2_1, fma(2.0 * oo2ze, v6_2_1, acc[22])));
+                acc[23] = fma(QCx, v12_3_0, fma(WQx, v12_3_1, fma(2.0 * oo2ze, v6_3_1, acc[23])));
+                acc[24] = fma(QCy, v12_2_0, fma(WQy, v12_2_1, fma(1.0 * oo2e, (v12_0_0 - rho_e * v12_0_1), acc[24])));
+                acc[25] = fma(QCy, v12_3_0, fma(WQy, v12_3_1, acc[25]));
+                acc[26] = fma(QCz, v12_3_0, fma(WQz, v12_3_1, fma(1.0 * oo2ze, v4_3_1, fma(1.0 * oo2e, (v12_0_0 - rho_e * v12_0_1), acc[26]))));
+                acc[27] += (double)v13_1_0;
+                acc[28] += (double)v13_2_0;
+                acc[29] += (double)v13_3_0;
+                acc[30] = fma(QCx, v13_1_0, fma(WQx, v13_1_1, fma(1.0 * oo2ze, v7_1_1, fma(1.0 * oo2e, (v13_0_0 - rho_e * v13_0_1), acc[30]))));
+                acc[31] = fma(QCx, v13_2_0, fma(WQx, v13_2_1, fma(1.0 * oo2ze, v7_2_1, acc[31])));
+                acc[32] = fma(QCx, v13_3_0, fma(WQx, v13_3_1, fma(1.0 * oo2ze, v7_3_1, acc[32])));
+                acc[33] = fma(QCy, v13_2_0, fma(WQy, v13_2_1, fma(2.0 * oo2ze, v5_2_1, fma(1.0 * oo2e, (v13_0_0 - rho_e * v13_0_1), acc[33]))));
+                acc[34] = fma(QCy, v13_3_0, fma(WQy, v13_3_1, fma(2.0 * oo2ze, v5_3_1, acc[34])));
+                acc[35] = fma(QCz, v13_3_0, fma(WQz, v13_3_1, fma(1.0 * oo2e, (v13_0_0 - rho_e * v13_0_1), acc[35])));
+                acc[36] += (double)v14_1_0;
+                acc[37] += (double)v14_2_0;
+                acc[38] += (double)v14_3_0;
+                acc[39] = fma(QCx, v14_1_0, fma(WQx, v14_1_1, fma(1.0 * oo2ze, v9_1_1, fma(1.0 * oo2e, (v14_0_0 - rho_e * v14_0_1), acc[39]))));
+                acc[40] = fma(QCx, v14_2_0, fma(WQx, v14_2_1, fma(1.0 * oo2ze, v9_2_1, acc[40])));
+                acc[41] = fma(QCx, v14_3_0, fma(WQx, v14_3_1, fma(1.0 * oo2ze, v9_3_1, acc[41])));
+                acc[42] = fma(QCy, v14_2_0, fma(WQy, v14_2_1, fma(1.0 * oo2e, (v14_0_0 - rho_e * v14_0_1), acc[42])));
+                acc[43] = fma(QCy, v14_3_0, fma(WQy, v14_3_1, acc[43]));
+                acc[44] = fma(QCz, v14_3_0, fma(WQz, v14_3_1, fma(2.0 * oo2ze, v6_3_1, fma(1.0 * oo2e, (v14_0_0 - rho_e * v14_0_1), acc[44]))));
+                acc[45] += (double)v15_1_0;
+                acc[46] += (double)v15_2_0;
+                acc[47] += (double)v15_3_0;
+                acc[48] = fma(QCx, v15_1_0, fma(WQx, v15_1_1, fma(1.0 * oo2ze, v8_1_1, fma(1.0 * oo2e, (v15_0_0 - rho_e * v15_0_1), acc[48]))));
+                acc[49] = fma(QCx, v15_2_0, fma(WQx, v15_2_1, fma(1.0 * oo2ze, v8_2_1, acc[49])));
+                acc[50] = fma(QCx, v15_3_0, fma(WQx, v15_3_1, fma(1.0 * oo2ze, v8_3_1, acc[50])));
+                acc[51] = fma(QCy, v15_2_0, fma(WQy, v15_2_1, fma(1.0 * oo2ze, v6_2_1, fma(1.0 * oo2e, (v15_0_0 - rho_e * v15_0_1), acc[51]))));
+                acc[52] = fma(QCy, v15_3_0, fma(WQy, v15_3_1, fma(1.0 * oo2ze, v6_3_1, acc[52])));
+                acc[53] = fma(QCz, v15_3_0, fma(WQz, v15_3_1, fma(1.0 * oo2ze, v5_3_1, fma(1.0 * oo2e, (v15_0_0 - rho_e * v15_0_1), acc[53]))));
+                acc[54] += (double)v16_1_0;
+                acc[55] += (double)v16_2_0;
+                acc[56] += (double)v16_3_0;
+                acc[57] = fma(QCx, v16_1_0, fma(WQx, v16_1_1, fma(1.0 * oo2e, (v16_0_0 - rho_e * v16_0_1), acc[57])));
+                acc[58] = fma(QCx, v16_2_0, fma(WQx, v16_2_1, acc[58]));
+                acc[59] = fma(QCx, v16_3_0, fma(WQx, v16_3_1, acc[59]));
+                acc[60] = fma(QCy, v16_2_0, fma(WQy, v16_2_1, fma(3.0 * oo2ze, v7_2_1, fma(1.0 * oo2e, (v16_0_0 - rho_e * v16_0_1), acc[60]))));
+                acc[61] = fma(QCy, v16_3_0, fma(WQy, v16_3_1, fma(3.0 * oo2ze, v7_3_1, acc[61])));
+                acc[62] = fma(QCz, v16_3_0, fma(WQz, v16_3_1, fma(1.0 * oo2e, (v16_0_0 - rho_e * v16_0_1), acc[62])));
+                acc[63] += (double)v17_1_0;
+                acc[64] += (double)v17_2_0;
+                acc[65] += (double)v17_3_0;
+                acc[66] = fma(QCx, v17_1_0, fma(WQx, v17_1_1, fma(1.0 * oo2e, (v17_0_0 - rho_e * v17_0_1), acc[66])));
+                acc[67] = fma(QCx, v17_2_0, fma(WQx, v17_2_1, acc[67]));
+                acc[68] = fma(QCx, v17_3_0, fma(WQx, v17_3_1, acc[68]));
+                acc[69] = fma(QCy, v17_2_0, fma(WQy, v17_2_1, fma(2.0 * oo2ze, v8_2_1, fma(1.0 * oo2e, (v17_0_0 - rho_e * v17_0_1), acc[69]))));
+                acc[70] = fma(QCy, v17_3_0, fma(WQy, v17_3_1, fma(2.0 * oo2ze, v8_3_1, acc[70])));
+                acc[71] = fma(QCz, v17_3_0, fma(WQz, v17_3_1, fma(1.0 * oo2ze, v7_3_1, fma(1.0 * oo2e, (v17_0_0 - rho_e * v17_0_1), acc[71]))));
+                acc[72] += (double)v18_1_0;
+                acc[73] += (double)v18_2_0;
+                acc[74] += (double)v18_3_0;
+                acc[75] = fma(QCx, v18_1_0, fma(WQx, v18_1_1, fma(1.0 * oo2e, (v18_0_0 - rho_e * v18_0_1), acc[75])));
+                acc[76] = fma(QCx, v18_2_0, fma(WQx, v18_2_1, acc[76]));
+                acc[77] = fma(QCx, v18_3_0, fma(WQx, v18_3_1, acc[77]));
+                acc[78] = fma(QCy, v18_2_0, fma(WQy, v18_2_1, fma(1.0 * oo2ze, v9_2_1, fma(1.0 * oo2e, (v18_0_0 - rho_e * v18_0_1), acc[78]))));
+                acc[79] = fma(QCy, v18_3_0, fma(WQy, v18_3_1, fma(1.0 * oo2ze, v9_3_1, acc[79])));
+                acc[80] = fma(QCz, v18_3_0, fma(WQz, v18_3_1, fma(2.0 * oo2ze, v8_3_1, fma(1.0 * oo2e, (v18_0_0 - rho_e * v18_0_1), acc[80]))));
+                acc[81] += (double)v19_1_0;
+                acc[82] += (double)v19_2_0;
+                acc[83] += (double)v19_3_0;
+                acc[84] = fma(QCx, v19_1_0, fma(WQx, v19_1_1, fma(1.0 * oo2e, (v19_0_0 - rho_e * v19_0_1), acc[84])));
+                acc[85] = fma(QCx, v19_2_0, fma(WQx, v19_2_1, acc[85]));
+                acc[86] = fma(QCx, v19_3_0, fma(WQx, v19_3_1, acc[86]));
+                acc[87] = fma(QCy, v19_2_0, fma(WQy, v19_2_1, fma(1.0 * oo2e, (v19_0_0 - rho_e * v19_0_1), acc[87])));
+                acc[88] = fma(QCy, v19_3_0, fma(WQy, v19_3_1, acc[88]));
+                acc[89] = fma(QCz, v19_3_0, fma(WQz, v19_3_1, fma(3.0 * oo2ze, v9_3_1, fma(1.0 * oo2e, (v19_0_0 - rho_e * v19_0_1), acc[89]))));
+                acc[90] += (double)v20_1_0;
+                acc[91] += (double)v20_2_0;
+                acc[92] += (double)v20_3_0;
+                acc[93] = fma(QCx, v20_1_0, fma(WQx, v20_1_1, fma(4.0 * oo2ze, v10_1_1, fma(1.0 * oo2e, (v20_0_0 - rho_e * v20_0_1), acc[93]))));
+                acc[94] = fma(QCx, v20_2_0, fma(WQx, v20_2_1, fma(4.0 * oo2ze, v10_2_1, acc[94])));
+                acc[95] = fma(QCx, v20_3_0, fma(WQx, v20_3_1, fma(4.0 * oo2ze, v10_3_1, acc[95])));
+                acc[96] = fma(QCy, v20_2_0, fma(WQy, v20_2_1, fma(1.0 * oo2e, (v20_0_0 - rho_e * v20_0_1), acc[96])));
+                acc[97] = fma(QCy, v20_3_0, fma(WQy, v20_3_1, acc[97]));
+                acc[98] = fma(QCz, v20_3_0, fma(WQz, v20_3_1, fma(1.0 * oo2e, (v20_0_0 - rho_e * v20_0_1), acc[98])));
+                acc[99] += (double)v21_1_0;
+                acc[100] += (double)v21_2_0;
+                acc[101] += (double)v21_3_0;
+                acc[102] = fma(QCx, v21_1_0, fma(WQx, v21_1_1, fma(3.0 * oo2ze, v11_1_1, fma(1.0 * oo2e, (v21_0_0 - rho_e * v21_0_1), acc[102]))));
+                acc[103] = fma(QCx, v21_2_0, fma(WQx, v21_2_1, fma(3.0 * oo2ze, v11_2_1, acc[103])));
+                acc[104] = fma(QCx, v21_3_0, fma(WQx, v21_3_1, fma(3.0 * oo2ze, v11_3_1, acc[104])));
+                acc[105] = fma(QCy, v21_2_0, fma(WQy, v21_2_1, fma(1.0 * oo2ze, v10_2_1, fma(1.0 * oo2e, (v21_0_0 - rho_e * v21_0_1), acc[105]))));
+                acc[106] = fma(QCy, v21_3_0, fma(WQy, v21_3_1, fma(1.0 * oo2ze, v10_3_1, acc[106])));
+                acc[107] = fma(QCz, v21_3_0, fma(WQz, v21_3_1, fma(1.0 * oo2e, (v21_0_0 - rho_e * v21_0_1), acc[107])));
+                acc[108] += (double)v22_1_0;
+                acc[109] += (double)v22_2_0;
+                acc[110] += (double)v22_3_0;
+                acc[111] = fma(QCx, v22_1_0, fma(WQx, v22_1_1, fma(3.0 * oo2ze, v12_1_1, fma(1.0 * oo2e, (v22_0_0 - rho_e * v22_0_1), acc[111]))));
+                acc[112] = fma(QCx, v22_2_0, fma(WQx, v22_2_1, fma(3.0 * oo2ze, v12_2_1, acc[112])));
+                acc[113] = fma(QCx, v22_3_0, fma(WQx, v22_3_1, fma(3.0 * oo2ze, v12_3_1, acc[113])));
+                acc[114] = fma(QCy, v22_2_0, fma(WQy, v22_2_1, fma(1.0 * oo2e, (v22_0_0 - rho_e * v22_0_1), acc[114])));
+                acc[115] = fma(QCy, v22_3_0, fma(WQy, v22_3_1, acc[115]));
+                acc[116] = fma(QCz, v22_3_0, fma(WQz, v22_3_1, fma(1.0 * oo2ze, v10_3_1, fma(1.0 * oo2e, (v22_0_0 - rho_e * v22_0_1), acc[116]))));
+                acc[117] += (double)v23_1_0;
+                acc[118] += (double)v23_2_0;
+                acc[119] += (double)v23_3_0;
+                acc[120] = fma(QCx, v23_1_0, fma(WQx, v23_1_1, fma(2.0 * oo2ze, v13_1_1, fma(1.0 * oo2e, (v23_0_0 - rho_e * v23_0_1), acc[120]))));
+                acc[121] = fma(QCx, v23_2_0, fma(WQx, v23_2_1, fma(2.0 * oo2ze, v13_2_1, acc[121])));
+                acc[122] = fma(QCx, v23_3_0, fma(WQx, v23_3_1, fma(2.0 * oo2ze, v13_3_1, acc[122])));
+                acc[123] = fma(QCy, v23_2_0, fma(WQy, v23_2_1, fma(2.0 * oo2ze, v11_2_1, fma(1.0 * oo2e, (v23_0_0 - rho_e * v23_0_1), acc[123]))));
+                acc[124] = fma(QCy, v23_3_0, fma(WQy, v23_3_1, fma(2.0 * oo2ze, v11_3_1, acc[124])));
+                acc[125] = fma(QCz, v23_3_0, fma(WQz, v23_3_1, fma(1.0 * oo2e, (v23_0_0 - rho_e * v23_0_1), acc[125])));
+                acc[126] += (double)v24_1_0;
+                acc[127] += (double)v24_2_0;
+                acc[128] += (double)v24_3_0;
+                acc[129] = fma(QCx, v24_1_0, fma(WQx, v24_1_1, fma(2.0 * oo2ze, v15_1_1, fma(1.0 * oo2e, (v24_0_0 - rho_e * v24_0_1), acc[129]))));
+                acc[130] = fma(QCx, v24_2_0, fma(WQx, v24_2_1, fma(2.0 * oo2ze, v15_2_1, acc[130])));
+                acc[131] = fma(QCx, v24_3_0, fma(WQx, v24_3_1, fma(2.0 * oo2ze, v15_3_1, acc[131])));
+                acc[132] = fma(QCy, v24_2_0, fma(WQy, v24_2_1, fma(1.0 * oo2ze, v12_2_1, fma(1.0 * oo2e, (v24_0_0 - rho_e * v24_0_1), acc[132]))));
+                acc[133] = fma(QCy, v24_3_0, fma(WQy, v24_3_1, fma(1.0 * oo2ze, v12_3_1, acc[133])));
+                acc[134] = fma(QCz, v24_3_0, fma(WQz, v24_3_1, fma(1.0 * oo2ze, v11_3_1, fma(1.0 * oo2e, (v24_0_0 - rho_e * v24_0_1), acc[134]))));
+                acc[135] += (double)v25_1_0;
+                acc[136] += (double)v25_2_0;
+                acc[137] += (double)v25_3_0;
+                acc[138] = fma(QCx, v25_1_0, fma(WQx, v25_1_1, fma(2.0 * oo2ze, v14_1_1, fma(1.0 * oo2e, (v25_0_0 - rho_e * v25_0_1), acc[138]))));
+                acc[139] = fma(QCx, v25_2_0, fma(WQx, v25_2_1, fma(2.0 * oo2ze, v14_2_1, acc[139])));
+                acc[140] = fma(QCx, v25_3_0, fma(WQx, v25_3_1, fma(2.0 * oo2ze, v14_3_1, acc[140])));
+                acc[141] = fma(QCy, v25_2_0, fma(WQy, v25_2_1, fma(1.0 * oo2e, (v25_0_0 - rho_e * v25_0_1), acc[141])));
+                acc[142] = fma(QCy, v25_3_0, fma(WQy, v25_3_1, acc[142]));
+                acc[143] = fma(QCz, v25_3_0, fma(WQz, v25_3_1, fma(2.0 * oo2ze, v12_3_1, fma(1.0 * oo2e, (v25_0_0 - rho_e * v25_0_1), acc[143]))));
+                acc[144] += (double)v26_1_0;
+                acc[145] += (double)v26_2_0;
+                acc[146] += (double)v26_3_0;
+                acc[147] = fma(QCx, v26_1_0, fma(WQx, v26_1_1, fma(1.0 * oo2ze, v16_1_1, fma(1.0 * oo2e, (v26_0_0 - rho_e * v26_0_1), acc[147]))));
+                acc[148] = fma(QCx, v26_2_0, fma(WQx, v26_2_1, fma(1.0 * oo2ze, v16_2_1, acc[148])));
+                acc[149] = fma(QCx, v26_3_0, fma(WQx, v26_3_1, fma(1.0 * oo2ze, v16_3_1, acc[149])));
+                acc[150] = fma(QCy, v26_2_0, fma(WQy, v26_2_1, fma(3.0 * oo2ze, v13_2_1, fma(1.0 * oo2e, (v26_0_0 - rho_e * v26_0_1), acc[150]))));
+                acc[151] = fma(QCy, v26_3_0, fma(WQy, v26_3_1, fma(3.0 * oo2ze, v13_3_1, acc[151])));
+                acc[152] = fma(QCz, v26_3_0, fma(WQz, v26_3_1, fma(1.0 * oo2e, (v26_0_0 - rho_e * v26_0_1), acc[152])));
+                acc[153] += (double)v27_1_0;
+                acc[154] += (double)v27_2_0;
+                acc[155] += (double)v27_3_0;
+                acc[156] = fma(QCx, v27_1_0, fma(WQx, v27_1_1, fma(1.0 * oo2ze, v17_1_1, fma(1.0 * oo2e, (v27_0_0 - rho_e * v27_0_1), acc[156]))));
+                acc[157] = fma(QCx, v27_2_0, fma(WQx, v27_2_1, fma(1.0 * oo2ze, v17_2_1, acc[157])));
+                acc[158] = fma(QCx, v27_3_0, fma(WQx, v27_3_1, fma(1.0 * oo2ze, v17_3_1, acc[158])));
+                acc[159] = fma(QCy, v27_2_0, fma(WQy, v27_2_1, fma(2.0 * oo2ze, v15_2_1, fma(1.0 * oo2e, (v27_0_0 - rho_e * v27_0_1), acc[159]))));
+                acc[160] = fma(QCy, v27_3_0, fma(WQy, v27_3_1, fma(2.0 * oo2ze, v15_3_1, acc[160])));
+                acc[161] = fma(QCz, v27_3_0, fma(WQz, v27_3_1, fma(1.0 * oo2ze, v13_3_1, fma(1.0 * oo2e, (v27_0_0 - rho_e * v27_0_1), acc[161]))));
+                acc[162] += (double)v28_1_0;
+                acc[163] += (double)v28_2_0;
+                acc[164] += (double)v28_3_0;
+                acc[165] = fma(QCx, v28_1_0, fma(WQx, v28_1_1, fma(1.0 * oo2ze, v18_1_1, fma(1.0 * oo2e, (v28_0_0 - rho_e * v28_0_1), acc[165]))));
+                acc[166] = fma(QCx, v28_2_0, fma(WQx, v28_2_1, fma(1.0 * oo2ze, v18_2_1, acc[166])));
+                acc[167] = fma(QCx, v28_3_0, fma(WQx, v28_3_1, fma(1.0 * oo2ze, v18_3_1, acc[167])));
+                acc[168] = fma(QCy, v28_2_0, fma(WQy, v28_2_1, fma(1.0 * oo2ze, v14_2_1, fma(1.0 * oo2e, (v28_0_0 - rho_e * v28_0_1), acc[168]))));
+                acc[169] = fma(QCy, v28_3_0, fma(WQy, v28_3_1, fma(1.0 * oo2ze, v14_3_1, acc[169])));
+                acc[170] = fma(QCz, v28_3_0, fma(WQz, v28_3_1, fma(2.0 * oo2ze, v15_3_1, fma(1.0 * oo2e, (v28_0_0 - rho_e * v28_0_1), acc[170]))));
+                acc[171] += (double)v29_1_0;
+                acc[172] += (double)v29_2_0;
+                acc[173] += (double)v29_3_0;
+                acc[174] = fma(QCx, v29_1_0, fma(WQx, v29_1_1, fma(1.0 * oo2ze, v19_1_1, fma(1.0 * oo2e, (v29_0_0 - rho_e * v29_0_1), acc[174]))));
+                acc[175] = fma(QCx, v29_2_0, fma(WQx, v29_2_1, fma(1.0 * oo2ze, v19_2_1, acc[175])));
+                acc[176] = fma(QCx, v29_3_0, fma(WQx, v29_3_1, fma(1.0 * oo2ze, v19_3_1, acc[176])));
+                acc[177] = fma(QCy, v29_2_0, fma(WQy, v29_2_1, fma(1.0 * oo2e, (v29_0_0 - rho_e * v29_0_1), acc[177])));
+                acc[178] = fma(QCy, v29_3_0, fma(WQy, v29_3_1, acc[178]));
+                acc[179] = fma(QCz, v29_3_0, fma(WQz, v29_3_1, fma(3.0 * oo2ze, v14_3_1, fma(1.0 * oo2e, (v29_0_0 - rho_e * v29_0_1), acc[179]))));
+                acc[180] += (double)v30_1_0;
+                acc[181] += (double)v30_2_0;
+                acc[182] += (double)v30_3_0;
+                acc[183] = fma(QCx, v30_1_0, fma(WQx, v30_1_1, fma(1.0 * oo2e, (v30_0_0 - rho_e * v30_0_1), acc[183])));
+                acc[184] = fma(QCx, v30_2_0, fma(WQx, v30_2_1, acc[184]));
+                acc[185] = fma(QCx, v30_3_0, fma(WQx, v30_3_1, acc[185]));
+                acc[186] = fma(QCy, v30_2_0, fma(WQy, v30_2_1, fma(4.0 * oo2ze, v16_2_1, fma(1.0 * oo2e, (v30_0_0 - rho_e * v30_0_1), acc[186]))));
+                acc[187] = fma(QCy, v30_3_0, fma(WQy, v30_3_1, fma(4.0 * oo2ze, v16_3_1, acc[187])));
+                acc[188] = fma(QCz, v30_3_0, fma(WQz, v30_3_1, fma(1.0 * oo2e, (v30_0_0 - rho_e * v30_0_1), acc[188])));
+                acc[189] += (double)v31_1_0;
+                acc[190] += (double)v31_2_0;
+                acc[191] += (double)v31_3_0;
+                acc[192] = fma(QCx, v31_1_0, fma(WQx, v31_1_1, fma(1.0 * oo2e, (v31_0_0 - rho_e * v31_0_1), acc[192])));
+                acc[193] = fma(QCx, v31_2_0, fma(WQx, v31_2_1, acc[193]));
+                acc[194] = fma(QCx, v31_3_0, fma(WQx, v31_3_1, acc[194]));
+                acc[195] = fma(QCy, v31_2_0, fma(WQy, v31_2_1, fma(3.0 * oo2ze, v17_2_1, fma(1.0 * oo2e, (v31_0_0 - rho_e * v31_0_1), acc[195]))));
+                acc[196] = fma(QCy, v31_3_0, fma(WQy, v31_3_1, fma(3.0 * oo2ze, v17_3_1, acc[196])));
+                acc[197] = fma(QCz, v31_3_0, fma(WQz, v31_3_1, fma(1.0 * oo2ze, v16_3_1, fma(1.0 * oo2e, (v31_0_0 - rho_e * v31_0_1), acc[197]))));
+                acc[198] += (double)v32_1_0;
+                acc[199] += (double)v32_2_0;
+                acc[200] += (double)v32_3_0;
+                acc[201] = fma(QCx, v32_1_0, fma(WQx, v32_1_1, fma(1.0 * oo2e, (v32_0_0 - rho_e * v32_0_1), acc[201])));
+                acc[202] = fma(QCx, v32_2_0, fma(WQx, v32_2_1, acc[202]));
+                acc[203] = fma(QCx, v32_3_0, fma(WQx, v32_3_1, acc[203]));
+                acc[204] = fma(QCy, v32_2_0, fma(WQy, v32_2_1, fma(2.0 * oo2ze, v18_2_1, fma(1.0 * oo2e, (v32_0_0 - rho_e * v32_0_1), acc[204]))));
+                acc[205] = fma(QCy, v32_3_0, fma(WQy, v32_3_1, fma(2.0 * oo2ze, v18_3_1, acc[205])));
+                acc[206] = fma(QCz, v32_3_0, fma(WQz, v32_3_1, fma(2.0 * oo2ze, v17_3_1, fma(1.0 * oo2e, (v32_0_0 - rho_e * v32_0_1), acc[206]))));
+                acc[207] += (double)v33_1_0;
+                acc[208] += (double)v33_2_0;
+                acc[209] += (double)v33_3_0;
+                acc[210] = fma(QCx, v33_1_0, fma(WQx, v33_1_1, fma(1.0 * oo2e, (v33_0_0 - rho_e * v33_0_1), acc[210])));
+                acc[211] = fma(QCx, v33_2_0, fma(WQx, v33_2_1, acc[211]));
+                acc[212] = fma(QCx, v33_3_0, fma(WQx, v33_3_1, acc[212]));
+                acc[213] = fma(QCy, v33_2_0, fma(WQy, v33_2_1, fma(1.0 * oo2ze, v19_2_1, fma(1.0 * oo2e, (v33_0_0 - rho_e * v33_0_1), acc[213]))));
+                acc[214] = fma(QCy, v33_3_0, fma(WQy, v33_3_1, fma(1.0 * oo2ze, v19_3_1, acc[214])));
+                acc[215] = fma(QCz, v33_3_0, fma(WQz, v33_3_1, fma(3.0 * oo2ze, v18_3_1, fma(1.0 * oo2e, (v33_0_0 - rho_e * v33_0_1), acc[215]))));
+                acc[216] += (double)v34_1_0;
+                acc[217] += (double)v34_2_0;
+                acc[218] += (double)v34_3_0;
+                acc[219] = fma(QCx, v34_1_0, fma(WQx, v34_1_1, fma(1.0 * oo2e, (v34_0_0 - rho_e * v34_0_1), acc[219])));
+                acc[220] = fma(QCx, v34_2_0, fma(WQx, v34_2_1, acc[220]));
+                acc[221] = fma(QCx, v34_3_0, fma(WQx, v34_3_1, acc[221]));
+                acc[222] = fma(QCy, v34_2_0, fma(WQy, v34_2_1, fma(1.0 * oo2e, (v34_0_0 - rho_e * v34_0_1), acc[222])));
+                acc[223] = fma(QCy, v34_3_0, fma(WQy, v34_3_1, acc[223]));
+                acc[224] = fma(QCz, v34_3_0, fma(WQz, v34_3_1, fma(4.0 * oo2ze, v19_3_1, fma(1.0 * oo2e, (v34_0_0 - rho_e * v34_0_1), acc[224]))));
+            } else {
+                acc[0] += (double)v10_1_0;
+                acc[1] += (double)v10_2_0;
+                acc[2] += (double)v10_3_0;
+                const VT v10_4_0 = QCx * v10_1_0 + WQx * v10_1_1 + (VT)3.0 * oo2ze * v4_1_1 + (VT)1.0 * oo2e * (v10_0_0 - rho_e * v10_0_1);
+                acc[3] += (double)v10_4_0;
+                const VT v10_5_0 = QCx * v10_2_0 + WQx * v10_2_1 + (VT)3.0 * oo2ze * v4_2_1;
+                acc[4] += (double)v10_5_0;
+                const VT v10_6_0 = QCx * v10_3_0 + WQx * v10_3_1 + (VT)3.0 * oo2ze * v4_3_1;
+                acc[5] += (double)v10_6_0;
+                const VT v10_7_0 = QCy * v10_2_0 + WQy * v10_2_1 + (VT)1.0 * oo2e * (v10_0_0 - rho_e * v10_0_1);
+                acc[6] += (double)v10_7_0;
+                const VT v10_8_0 = QCy * v10_3_0 + WQy * v10_3_1;
+                acc[7] += (double)v10_8_0;
+                const VT v10_9_0 = QCz * v10_3_0 + WQz * v10_3_1 + (VT)1.0 * oo2e * (v10_0_0 - rho_e * v10_0_1);
+                acc[8] += (double)v10_9_0;
+                acc[9] += (double)v11_1_0;
+                acc[10] += (double)v11_2_0;
+                acc[11] += (double)v11_3_0;
+                const VT v11_4_0 = QCx * v11_1_0 + WQx * v11_1_1 + (VT)2.0 * oo2ze * v5_1_1 + (VT)1.0 * oo2e * (v11_0_0 - rho_e * v11_0_1);
+                acc[12] += (double)v11_4_0;
+                const VT v11_5_0 = QCx * v11_2_0 + WQx * v11_2_1 + (VT)2.0 * oo2ze * v5_2_1;
+                acc[13] += (double)v11_5_0;
+                const VT v11_6_0 = QCx * v11_3_0 + WQx * v11_3_1 + (VT)2.0 * oo2ze * v5_3_1;
+                acc[14] += (double)v11_6_0;
+                const VT v11_7_0 = QCy * v11_2_0 + WQy * v11_2_1 + (VT)1.0 * oo2ze * v4_2_1 + (VT)1.0 * oo2e * (v11_0_0 - rho_e * v11_0_1);
+                acc[15] += (double)v11_7_0;
+                const VT v11_8_0 = QCy * v11_3_0 + WQy * v11_3_1 + (VT)1.0 * oo2ze * v4_3_1;
+                acc[16] += (double)v11_8_0;
+                const VT v11_9_0 = QCz * v11_3_0 + WQz * v11_3_1 + (VT)1.0 * oo2e * (v11_0_0 - rho_e * v11_0_1);
+                acc[17] += (double)v11_9_0;
+                acc[18] += (double)v12_1_0;
+                acc[19] += (double)v12_2_0;
+                acc[20] += (double)v12_3_0;
+                const VT v12_4_0 = QCx * v12_1_0 + WQx * v12_1_1 + (VT)2.0 * oo2ze * v6_1_1 + (VT)1.0 * oo2e * (v12_0_0 - rho_e * v12_0_1);
+                acc[21] += (double)v12_4_0;
+                const VT v12_5_0 = QCx * v12_2_0 + WQx * v12_2_1 + (VT)2.0 * oo2ze * v6_2_1;
+                acc[22] += (double)v12_5_0;
+                const VT v12_6_0 = QCx * v12_3_0 + WQx * v12_3_1 + (VT)2.0 * oo2ze * v6_3_1;
+                acc[23] += (double)v12_6_0;
+                const VT v12_7_0 = QCy * v12_2_0 + WQy * v12_2_1 + (VT)1.0 * oo2e * (v12_0_0 - rho_e * v12_0_1);
+                acc[24] += (double)v12_7_0;
+                const VT v12_8_0 = QCy * v12_3_0 + WQy * v12_3_1;
+                acc[25] += (double)v12_8_0;
+                const VT v12_9_0 = QCz * v12_3_0 + WQz * v12_3_1 + (VT)1.0 * oo2ze * v4_3_1 + (VT)1.0 * oo2e * (v12_0_0 - rho_e * v12_0_1);
+                acc[26] += (double)v12_9_0;
+                acc[27] += (double)v13_1_0;
+                acc[28] += (double)v13_2_0;
+                acc[29] += (double)v13_3_0;
+                const VT v13_4_0 = QCx * v13_1_0 + WQx * v13_1_1 + (VT)1.0 * oo2ze * v7_1_1 + (VT)1.0 * oo2e * (v13_0_0 - rho_e * v13_0_1);
+                acc[30] += (double)v13_4_0;
+                const VT v13_5_0 = QCx * v13_2_0 + WQx * v13_2_1 + (VT)1.0 * oo2ze * v7_2_1;
+                acc[31] += (double)v13_5_0;
+                const VT v13_6_0 = QCx * v13_3_0 + WQx * v13_3_1 + (VT)1.0 * oo2ze * v7_3_1;
+                acc[32] += (double)v13_6_0;
+                const VT v13_7_0 = QCy * v13_2_0 + WQy * v13_2_1 + (VT)2.0 * oo2ze * v5_2_1 + (VT)1.0 * oo2e * (v13_0_0 - rho_e * v13_0_1);
+                acc[33] += (double)v13_7_0;
+                const VT v13_8_0 = QCy * v13_3_0 + WQy * v13_3_1 + (VT)2.0 * oo2ze * v5_3_1;
+                acc[34] += (double)v13_8_0;
+                const VT v13_9_0 = QCz * v13_3_0 + WQz * v13_3_1 + (VT)1.0 * oo2e * (v13_0_0 - rho_e * v13_0_1);
+                acc[35] += (double)v13_9_0;
+                acc[36] += (double)v14_1_0;
+                acc[37] += (double)v14_2_0;
+                acc[38] += (double)v14_3_0;
+                const VT v14_4_0 = QCx * v14_1_0 + WQx * v14_1_1 + (VT)1.0 * oo2ze * v9_1_1 + (VT)1.0 * oo2e * (v14_0_0 - rho_e * v14_0_1);
+                acc[39] += (double)v14_4_0;
+                const VT v14_5_0 = QCx * v14_2_0 + WQx * v14_2_1 + (VT)1.0 * oo2ze * v9_2_1;
+                acc[40] += (double)v14_5_0;
+                const VT v14_6_0 = QCx * v14_3_0 + WQx * v14_3_1 + (VT)1.0 * oo2ze * v9_3_1;
+                acc[41] += (double)v14_6_0;
+                const VT v14_7_0 = QCy * v14_2_0 + WQy * v14_2_1 + (VT)1.0 * oo2e * (v14_0_0 - rho_e * v14_0_1);
+                acc[42] += (double)v14_7_0;
+                const VT v14_8_0 = QCy * v14_3_0 + WQy * v14_3_1;
+                acc[43] += (double)v14_8_0;
+                const VT v14_9_0 = QCz * v14_3_0 + WQz * v14_3_1 + (VT)2.0 * oo2ze * v6_3_1 + (VT)1.0 * oo2e * (v14_0_0 - rho_e * v14_0_1);
+                acc[44] += (double)v14_9_0;
+                acc[45] += (double)v15_1_0;
+                acc[46] += (double)v15_2_0;
+                acc[47] += (double)v15_3_0;
+                const VT v15_4_0 = QCx * v15_1_0 + WQx * v15_1_1 + (VT)1.0 * oo2ze * v8_1_1 + (VT)1.0 * oo2e * (v15_0_0 - rho_e * v15_0_1);
+                acc[48] += (double)v15_4_0;
+                const VT v15_5_0 = QCx * v15_2_0 + WQx * v15_2_1 + (VT)1.0 * oo2ze * v8_2_1;
+                acc[49] += (double)v15_5_0;
+                const VT v15_6_0 = QCx * v15_3_0 + WQx * v15_3_1 + (VT)1.0 * oo2ze * v8_3_1;
+                acc[50] += (double)v15_6_0;
+                const VT v15_7_0 = QCy * v15_2_0 + WQy * v15_2_1 + (VT)1.0 * oo2ze * v6_2_1 + (VT)1.0 * oo2e * (v15_0_0 - rho_e * v15_0_1);
+                acc[51] += (double)v15_7_0;
+                const VT v15_8_0 = QCy * v15_3_0 + WQy * v15_3_1 + (VT)1.0 * oo2ze * v6_3_1;
+                acc[52] += (double)v15_8_0;
+                const VT v15_9_0 = QCz * v15_3_0 + WQz * v15_3_1 + (VT)1.0 * oo2ze * v5_3_1 + (VT)1.0 * oo2e * (v15_0_0 - rho_e * v15_0_1);
+                acc[53] += (double)v15_9_0;
+                acc[54] += (double)v16_1_0;
+                acc[55] += (double)v16_2_0;
+                acc[56] += (double)v16_3_0;
+                const VT v16_4_0 = QCx * v16_1_0 + WQx * v16_1_1 + (VT)1.0 * oo2e * (v16_0_0 - rho_e * v16_0_1);
+                acc[57] += (double)v16_4_0;
+                const VT v16_5_0 = QCx * v16_2_0 + WQx * v16_2_1;
+                acc[58] += (double)v16_5_0;
+                const VT v16_6_0 = QCx * v16_3_0 + WQx * v16_3_1;
+                acc[59] += (double)v16_6_0;
+                const VT v16_7_0 = QCy * v16_2_0 + WQy * v16_2_1 + (VT)3.0 * oo2ze * v7_2_1 + (VT)1.0 * oo2e * (v16_0_0 - rho_e * v16_0_1);
+                acc[60] += (double)v16_7_0;
+                const VT v16_8_0 = QCy * v16_3_0 + WQy * v16_3_1 + (VT)3.0 * oo2ze * v7_3_1;
+                acc[61] += (double)v16_8_0;
+                const VT v16_9_0 = QCz * v16_3_0 + WQz * v16_3_1 + (VT)1.0 * oo2e * (v16_0_0 - rho_e * v16_0_1);
+                acc[62] += (double)v16_9_0;
+                acc[63] += (double)v17_1_0;
+                acc[64] += (double)v17_2_0;
+                acc[65] += (double)v17_3_0;
+                const VT v17_4_0 = QCx * v17_1_0 + WQx * v17_1_1 + (VT)1.0 * oo2e * (v17_0_0 - rho_e * v17_0_1);
+                acc[66] += (double)v17_4_0;
+                const VT v17_5_0 = QCx * v17_2_0 + WQx * v17_2_1;
+                acc[67] += (double)v17_5_0;
+                const VT v17_6_0 = QCx * v17_3_0 + WQx * v17_3_1;
+                acc[68] += (double)v17_6_0;
+                const VT v17_7_0 = QCy * v17_2_0 + WQy * v17_2_1 + (VT)2.0 * oo2ze * v8_2_1 + (VT)1.0 * oo2e * (v17_0_0 - rho_e * v17_0_1);
+                acc[69] += (double)v17_7_0;
+                const VT v17_8_0 = QCy * v17_3_0 + WQy * v17_3_1 + (VT)2.0 * oo2ze * v8_3_1;
+                acc[70] += (double)v17_8_0;
+                const VT v17_9_0 = QCz * v17_3_0 + WQz * v17_3_1 + (VT)1.0 * oo2ze * v7_3_1 + (VT)1.0 * oo2e * (v17_0_0 - rho_e * v17_0_1);
+                acc[71] += (double)v17_9_0;
+                acc[72] += (double)v18_1_0;
+                acc[73] += (double)v18_2_0;
+                acc[74] += (double)v18_3_0;
+                const VT v18_4_0 = QCx * v18_1_0 + WQx * v18_1_1 + (VT)1.0 * oo2e * (v18_0_0 - rho_e * v18_0_1);
+                acc[75] += (double)v18_4_0;
+                const VT v18_5_0 = QCx * v18_2_0 + WQx * v18_2_1;
+                acc[76] += (double)v18_5_0;
+                const VT v18_6_0 = QCx * v18_3_0 + WQx * v18_3_1;
+                acc[77] += (double)v18_6_0;
+                const VT v18_7_0 = QCy * v18_2_0 + WQy * v18_2_1 + (VT)1.0 * oo2ze * v9_2_1 + (VT)1.0 * oo2e * (v18_0_0 - rho_e * v18_0_1);
+                acc[78] += (double)v18_7_0;
+                const VT v18_8_0 = QCy * v18_3_0 + WQy * v18_3_1 + (VT)1.0 * oo2ze * v9_3_1;
+                acc[79] += (double)v18_8_0;
+                const VT v18_9_0 = QCz * v18_3_0 + WQz * v18_3_1 + (VT)2.0 * oo2ze * v8_3_1 + (VT)1.0 * oo2e * (v18_0_0 - rho_e * v18_0_1);
+                acc[80] += (double)v18_9_0;
+                acc[81] += (double)v19_1_0;
+                acc[82] += (double)v19_2_0;
+                acc[83] += (double)v19_3_0;
+                const VT v19_4_0 = QCx * v19_1_0 + WQx * v19_1_1 + (VT)1.0 * oo2e * (v19_0_0 - rho_e * v19_0_1);
+                acc[84] += (double)v19_4_0;
+                const VT v19_5_0 = QCx * v19_2_0 + WQx * v19_2_1;
+                acc[85] += (double)v19_5_0;
+                const VT v19_6_0 = QCx * v19_3_0 + WQx * v19_3_1;
+                acc[86] += (double)v19_6_0;
+                const VT v19_7_0 = QCy * v19_2_0 + WQy * v19_2_1 + (VT)1.0 * oo2e * (v19_0_0 - rho_e * v19_0_1);
+                acc[87] += (double)v19_7_0;
+                const VT v19_8_0 = QCy * v19_3_0 + WQy * v19_3_1;
+                acc[88] += (double)v19_8_0;
+                const VT v19_9_0 = QCz * v19_3_0 + WQz * v19_3_1 + (VT)3.0 * oo2ze * v9_3_1 + (VT)1.0 * oo2e * (v19_0_0 - rho_e * v19_0_1);
+                acc[89] += (double)v19_9_0;
+                acc[90] += (double)v20_1_0;
+                acc[91] += (double)v20_2_0;
+                acc[92] += (double)v20_3_0;
+                const VT v20_4_0 = QCx * v20_1_0 + WQx * v20_1_1 + (VT)4.0 * oo2ze * v10_1_1 + (VT)1.0 * oo2e * (v20_0_0 - rho_e * v20_0_1);
+                acc[93] += (double)v20_4_0;
+                const VT v20_5_0 = QCx * v20_2_0 + WQx * v20_2_1 + (VT)4.0 * oo2ze * v10_2_1;
+                acc[94] += (double)v20_5_0;
+                const VT v20_6_0 = QCx * v20_3_0 + WQx * v20_3_1 + (VT)4.0 * oo2ze * v10_3_1;
+                acc[95] += (double)v20_6_0;
+                const VT v20_7_0 = QCy * v20_2_0 + WQy * v20_2_1 + (VT)1.0 * oo2e * (v20_0_0 - rho_e * v20_0_1);
+                acc[96] += (double)v20_7_0;
+                const VT v20_8_0 = QCy * v20_3_0 + WQy * v20_3_1;
+                acc[97] += (double)v20_8_0;
+                const VT v20_9_0 = QCz * v20_3_0 + WQz * v20_3_1 + (VT)1.0 * oo2e * (v20_0_0 - rho_e * v20_0_1);
+                acc[98] += (double)v20_9_0;
+                acc[99] += (double)v21_1_0;
+                acc[100] += (double)v21_2_0;
+                acc[101] += (double)v21_3_0;
+                const VT v21_4_0 = QCx * v21_1_0 + WQx * v21_1_1 + (VT)3.0 * oo2ze * v11_1_1 + (VT)1.0 * oo2e * (v21_0_0 - rho_e * v21_0_1);
+                acc[102] += (double)v21_4_0;
+                const VT v21_5_0 = QCx * v21_2_0 + WQx * v21_2_1 + (VT)3.0 * oo2ze * v11_2_1;
+                acc[103] += (double)v21_5_0;
+                const VT v21_6_0 = QCx * v21_3_0 + WQx * v21_3_1 + (VT)3.0 * oo2ze * v11_3_1;
+                acc[104] += (double)v21_6_0;
+                const VT v21_7_0 = QCy * v21_2_0 + WQy * v21_2_1 + (VT)1.0 * oo2ze * v10_2_1 + (VT)1.0 * oo2e * (v21_0_0 - rho_e * v21_0_1);
+                acc[105] += (double)v21_7_0;
+                const VT v21_8_0 = QCy * v21_3_0 + WQy * v21_3_1 + (VT)1.0 * oo2ze * v10_3_1;
+                acc[106] += (double)v21_8_0;
+                const VT v21_9_0 = QCz * v21_3_0 + WQz * v21_3_1 + (VT)1.0 * oo2e * (v21_0_0 - rho_e * v21_0_1);
+                acc[107] += (double)v21_9_0;
+                acc[108] += (double)v22_1_0;
+                acc[109] += (double)v22_2_0;
+                acc[110] += (double)v22_3_0;
+                const VT v22_4_0 = QCx * v22_1_0 + WQx * v22_1_1 + (VT)3.0 * oo2ze * v12_1_1 + (VT)1.0 * oo2e * (v22_0_0 - rho_e * v22_0_1);
+                acc[111] += (double)v22_4_0;
+                const VT v22_5_0 = QCx * v22_2_0 + WQx * v22_2_1 + (VT)3.0 * oo2ze * v12_2_1;
+                acc[112] += (double)v22_5_0;
+                const VT v22_6_0 = QCx * v22_3_0 + WQx * v22_3_1 + (VT)3.0 * oo2ze * v12_3_1;
+                acc[113] += (double)v22_6_0;
+                const VT v22_7_0 = QCy * v22_2_0 + WQy * v22_2_1 + (VT)1.0 * oo2e * (v22_0_0 - rho_e * v22_0_1);
+                acc[114] += (double)v22_7_0;
+                const VT v22_8_0 = QCy * v22_3_0 + WQy * v22_3_1;
+                acc[115] += (double)v22_8_0;
+                const VT v22_9_0 = QCz * v22_3_0 + WQz * v22_3_1 + (VT)1.0 * oo2ze * v10_3_1 + (VT)1.0 * oo2e * (v22_0_0 - rho_e * v22_0_1);
+                acc[116] += (double)v22_9_0;
+                acc[117] += (double)v23_1_0;
+                acc[118] += (double)v23_2_0;
+                acc[119] += (double)v23_3_0;
+                const VT v23_4_0 = QCx * v23_1_0 + WQx * v23_1_1 + (VT)2.0 * oo2ze * v13_1_1 + (VT)1.0 * oo2e * (v23_0_0 - rho_e * v23_0_1);
+                acc[120] += (double)v23_4_0;
+                const VT v23_5_0 = QCx * v23_2_0 + WQx * v23_2_1 + (VT)2.0 * oo2ze * v13_2_1;
+                acc[121] += (double)v23_5_0;
+                const VT v23_6_0 = QCx * v23_3_0 + WQx * v23_3_1 + (VT)2.0 * oo2ze * v13_3_1;
+                acc[122] += (double)v23_6_0;
+                const VT v23_7_0 = QCy * v23_2_0 + WQy * v23_2_1 + (VT)2.0 * oo2ze * v11_2_1 + (VT)1.0 * oo2e * (v23_0_0 - rho_e * v23_0_1);
+                acc[123] += (double)v23_7_0;
+                const VT v23_8_0 = QCy * v23_3_0 + WQy * v23_3_1 + (VT)2.0 * oo2ze * v11_3_1;
+                acc[124] += (double)v23_8_0;
+                const VT v23_9_0 = QCz * v23_3_0 + WQz * v23_3_1 + (VT)1.0 * oo2e * (v23_0_0 - rho_e * v23_0_1);
+                acc[125] += (double)v23_9_0;
+                acc[126] += (double)v24_1_0;
+                acc[127] += (double)v24_2_0;
+                acc[128] += (double)v24_3_0;
+                const VT v24_4_0 = QCx * v24_1_0 + WQx * v24_1_1 + (VT)2.0 * oo2ze * v15_1_1 + (VT)1.0 * oo2e * (v24_0_0 - rho_e * v24_0_1);
+                acc[129] += (double)v24_4_0;
+                const VT v24_5_0 = QCx * v24_2_0 + WQx * v24_2_1 + (VT)2.0 * oo2ze * v15_2_1;
+                acc[130] += (double)v24_5_0;
+                const VT v24_6_0 = QCx * v24_3_0 + WQx * v24_3_1 + (VT)2.0 * oo2ze * v15_3_1;
+                acc[131] += (double)v24_6_0;
+                const VT v24_7_0 = QCy * v24_2_0 + WQy * v24_2_1 + (VT)1.0 * oo2ze * v12_2_1 + (VT)1.0 * oo2e * (v24_0_0 - rho_e * v24_0_1);
+                acc[132] += (double)v24_7_0;
+                const VT v24_8_0 = QCy * v24_3_0 + WQy * v24_3_1 + (VT)1.0 * oo2ze * v12_3_1;
+                acc[133] += (double)v24_8_0;
+                const VT v24_9_0 = QCz * v24_3_0 + WQz * v24_3_1 + (VT)1.0 * oo2ze * v11_3_1 + (VT)1.0 * oo2e * (v24_0_0 - rho_e * v24_0_1);
+                acc[134] += (double)v24_9_0;
+                acc[135] += (double)v25_1_0;
+                acc[136] += (double)v25_2_0;
+                acc[137] += (double)v25_3_0;
+                const VT v25_4_0 = QCx * v25_1_0 + WQx * v25_1_1 + (VT)2.0 * oo2ze * v14_1_1 + (VT)1.0 * oo2e * (v25_0_0 - rho_e * v25_0_1);
+                acc[138] += (double)v25_4_0;
+                const VT v25_5_0 = QCx * v25_2_0 + WQx * v25_2_1 + (VT)2.0 * oo2ze * v14_2_1;
+                acc[139] += (double)v25_5_0;
+                const VT v25_6_0 = QCx * v25_3_0 + WQx * v25_3_1 + (VT)2.0 * oo2ze * v14_3_1;
+                acc[140] += (double)v25_6_0;
+                const VT v25_7_0 = QCy * v25_2_0 + WQy * v25_2_1 + (VT)1.0 * oo2e * (v25_0_0 - rho_e * v25_0_1);
+                acc[141] += (double)v25_7_0;
+                const VT v25_8_0 = QCy * v25_3_0 + WQy * v25_3_1;
+                acc[142] += (double)v25_8_0;
+                const VT v25_9_0 = QCz * v25_3_0 + WQz * v25_3_1 + (VT)2.0 * oo2ze * v12_3_1 + (VT)1.0 * oo2e * (v25_0_0 - rho_e * v25_0_1);
+                acc[143] += (double)v25_9_0;
+                acc[144] += (double)v26_1_0;
+                acc[145] += (double)v26_2_0;
+                acc[146] += (double)v26_3_0;
+                const VT v26_4_0 = QCx * v26_1_0 + WQx * v26_1_1 + (VT)1.0 * oo2ze * v16_1_1 + (VT)1.0 * oo2e * (v26_0_0 - rho_e * v26_0_1);
+                acc[147] += (double)v26_4_0;
+                const VT v26_5_0 = QCx * v26_2_0 + WQx * v26_2_1 + (VT)1.0 * oo2ze * v16_2_1;
+                acc[148] += (double)v26_5_0;
+                const VT v26_6_0 = QCx * v26_3_0 + WQx * v26_3_1 + (VT)1.0 * oo2ze * v16_3_1;
+                acc[149] += (double)v26_6_0;
+                const VT v26_7_0 = QCy * v26_2_0 + WQy * v26_2_1 + (VT)3.0 * oo2ze * v13_2_1 + (VT)1.0 * oo2e * (v26_0_0 - rho_e * v26_0_1);
+                acc[150] += (double)v26_7_0;
+                const VT v26_8_0 = QCy * v26_3_0 + WQy * v26_3_1 + (VT)3.0 * oo2ze * v13_3_1;
+                acc[151] += (double)v26_8_0;
+                const VT v26_9_0 = QCz * v26_3_0 + WQz * v26_3_1 + (VT)1.0 * oo2e * (v26_0_0 - rho_e * v26_0_1);
+                acc[152] += (double)v26_9_0;
+                acc[153] += (double)v27_1_0;
+                acc[154] += (double)v27_2_0;
+                acc[155] += (double)v27_3_0;
+                const VT v27_4_0 = QCx * v27_1_0 + WQx * v27_1_1 + (VT)1.0 * oo2ze * v17_1_1 + (VT)1.0 * oo2e * (v27_0_0 - rho_e * v27_0_1);
+                acc[156] += (double)v27_4_0;
+                const VT v27_5_0 = QCx * v27_2_0 + WQx * v27_2_1 + (VT)1.0 * oo2ze * v17_2_1;
+                acc[157] += (double)v27_5_0;
+                const VT v27_6_0 = QCx * v27_3_0 + WQx * v27_3_1 + (VT)1.0 * oo2ze * v17_3_1;
+                acc[158] += (double)v27_6_0;
+                const VT v27_7_0 = QCy * v27_2_0 + WQy * v27_2_1 + (VT)2.0 * oo2ze * v15_2_1 + (VT)1.0 * oo2e * (v27_0_0 - rho_e * v27_0_1);
+                acc[159] += (double)v27_7_0;
+                const VT v27_8_0 = QCy * v27_3_0 + WQy * v27_3_1 + (VT)2.0 * oo2ze * v15_3_1;
+                acc[160] += (double)v27_8_0;
+                const VT v27_9_0 = QCz * v27_3_0 + WQz * v27_3_1 + (VT)1.0 * oo2ze * v13_3_1 + (VT)1.0 * oo2e * (v27_0_0 - rho_e * v27_0_1);
+                acc[161] += (double)v27_9_0;
+                acc[162] += (double)v28_1_0;
+                acc[163] += (double)v28_2_0;
+                acc[164] += (double)v28_3_0;
+                const VT v28_4_0 = QCx * v28_1_0 + WQx * v28_1_1 + (VT)1.0 * oo2ze * v18_1_1 + (VT)1.0 * oo2e * (v28_0_0 - rho_e * v28_0_1);
+                acc[165] += (double)v28_4_0;
+                const VT v28_5_0 = QCx * v28_2_0 + WQx * v28_2_1 + (VT)1.0 * oo2ze * v18_2_1;
+                acc[166] += (double)v28_5_0;
+                const VT v28_6_0 = QCx * v28_3_0 + WQx * v28_3_1 + (VT)1.0 * oo2ze * v18_3_1;
+                acc[167] += (double)v28_6_0;
+                const VT v28_7_0 = QCy * v28_2_0 + WQy * v28_2_1 + (VT)1.0 * oo2ze * v14_2_1 + (VT)1.0 * oo2e * (v28_0_0 - rho_e * v28_0_1);
+                acc[168] += (double)v28_7_0;
+                const VT v28_8_0 = QCy * v28_3_0 + WQy * v28_3_1 + (VT)1.0 * oo2ze * v14_3_1;
+                acc[169] += (double)v28_8_0;
+                const VT v28_9_0 = QCz * v28_3_0 + WQz * v28_3_1 + (VT)2.0 * oo2ze * v15_3_1 + (VT)1.0 * oo2e * (v28_0_0 - rho_e * v28_0_1);
+                acc[170] += (double)v28_9_0;
+                acc[171] += (double)v29_1_0;
+                acc[172] += (double)v29_2_0;
+                acc[173] += (double)v29_3_0;
+                const VT v29_4_0 = QCx * v29_1_0 + WQx * v29_1_1 + (VT)1.0 * oo2ze * v19_1_1 + (VT)1.0 * oo2e * (v29_0_0 - rho_e * v29_0_1);
+                acc[174] += (double)v29_4_0;
+                const VT v29_5_0 = QCx * v29_2_0 + WQx * v29_2_1 + (VT)1.0 * oo2ze * v19_2_1;
+                acc[175] += (double)v29_5_0;
+                const VT v29_6_0 = QCx * v29_3_0 + WQx * v29_3_1 + (VT)1.0 * oo2ze * v19_3_1;
+                acc[176] += (double)v29_6_0;
+                const VT v29_7_0 = QCy * v29_2_0 + WQy * v29_2_1 + (VT)1.0 * oo2e * (v29_0_0 - rho_e * v29_0_1);
+                acc[177] += (double)v29_7_0;
+                const VT v29_8_0 = QCy * v29_3_0 + WQy * v29_3_1;
+                acc[178] += (double)v29_8_0;
+                const VT v29_9_0 = QCz * v29_3_0 + WQz * v29_3_1 + (VT)3.0 * oo2ze * v14_3_1 + (VT)1.0 * oo2e * (v29_0_0 - rho_e * v29_0_1);
+                acc[179] += (double)v29_9_0;
+                acc[180] += (double)v30_1_0;
+                acc[181] += (double)v30_2_0;
+                acc[182] += (double)v30_3_0;
+                const VT v30_4_0 = QCx * v30_1_0 + WQx * v30_1_1 + (VT)1.0 * oo2e * (v30_0_0 - rho_e * v30_0_1);
+                acc[183] += (double)v30_4_0;
+                const VT v30_5_0 = QCx * v30_2_0 + WQx * v30_2_1;
+                acc[184] += (double)v30_5_0;
+                const VT v30_6_0 = QCx * v30_3_0 + WQx * v30_3_1;
+                acc[185] += (double)v30_6_0;
+                const VT v30_7_0 = QCy * v30_2_0 + WQy * v30_2_1 + (VT)4.0 * oo2ze * v16_2_1 + (VT)1.0 * oo2e * (v30_0_0 - rho_e * v30_0_1);
+                acc[186] += (double)v30_7_0;
+                const VT v30_8_0 = QCy * v30_3_0 + WQy * v30_3_1 + (VT)4.0 * oo2ze * v16_3_1;
+                acc[187] += (double)v30_8_0;
+                const VT v30_9_0 = QCz * v30_3_0 + WQz * v30_3_1 + (VT)1.0 * oo2e * (v30_0_0 - rho_e * v30_0_1);
+                acc[188] += (double)v30_9_0;
+                acc[189] += (double)v31_1_0;
+                acc[190] += (double)v31_2_0;
+                acc[191] += (double)v31_3_0;
+                const VT v31_4_0 = QCx * v31_1_0 + WQx * v31_1_1 + (VT)1.0 * oo2e * (v31_0_0 - rho_e * v31_0_1);
+                acc[192] += (double)v31_4_0;
+                const VT v31_5_0 = QCx * v31_2_0 + WQx * v31_2_1;
+                acc[193] += (double)v31_5_0;
+                const VT v31_6_0 = QCx * v31_3_0 + WQx * v31_3_1;
+                acc[194] += (double)v31_6_0;
+                const VT v31_7_0 = QCy * v31_2_0 + WQy * v31_2_1 + (VT)3.0 * oo2ze * v17_2_1 + (VT)1.0 * oo2e * (v31_0_0 - rho_e * v31_0_1);
+                acc[195] += (double)v31_7_0;
+                const VT v31_8_0 = QCy * v31_3_0 + WQy * v31_3_1 + (VT)3.0 * oo2ze * v17_3_1;
+                acc[196] += (double)v31_8_0;
+                const VT v31_9_0 = QCz * v31_3_0 + WQz * v31_3_1 + (VT)1.0 * oo2ze * v16_3_1 + (VT)1.0 * oo2e * (v31_0_0 - rho_e * v31_0_1);
+                acc[197] += (double)v31_9_0;
+                acc[198] += (double)v32_1_0;
+                acc[199] += (double)v32_2_0;
+                acc[200] += (double)v32_3_0;
+                const VT v32_4_0 = QCx * v32_1_0 + WQx * v32_1_1 + (VT)1.0 * oo2e * (v32_0_0 - rho_e * v32_0_1);
+                acc[201] += (double)v32_4_0;
+                const VT v32_5_0 = QCx * v32_2_0 + WQx * v32_2_1;
+                acc[202] += (double)v32_5_0;
+                const VT v32_6_0 = QCx * v32_3_0 + WQx * v32_3_1;
+                acc[203] += (double)v32_6_0;
+                const VT v32_7_0 = QCy * v32_2_0 + WQy * v32_2_1 + (VT)2.0 * oo2ze * v18_2_1 + (VT)1.0 * oo2e * (v32_0_0 - rho_e * v32_0_1);
+                acc[204] += (double)v32_7_0;
+                const VT v32_8_0 = QCy * v32_3_0 + WQy * v32_3_1 + (VT)2.0 * oo2ze * v18_3_1;
+                acc[205] += (double)v32_8_0;
+                const VT v32_9_0 = QCz * v32_3_0 + WQz * v32_3_1 + (VT)2.0 * oo2ze * v17_3_1 + (VT)1.0 * oo2e * (v32_0_0 - rho_e * v32_0_1);
+                acc[206] += (double)v32_9_0;
+                acc[207] += (double)v33_1_0;
+                acc[208] += (double)v33_2_0;
+                acc[209] += (double)v33_3_0;
+                const VT v33_4_0 = QCx * v33_1_0 + WQx * v33_1_1 + (VT)1.0 * oo2e * (v33_0_0 - rho_e * v33_0_1);
+                acc[210] += (double)v33_4_0;
+                const VT v33_5_0 = QCx * v33_2_0 + WQx * v33_2_1;
+                acc[211] += (double)v33_5_0;
+                const VT v33_6_0 = QCx * v33_3_0 + WQx * v33_3_1;
+                acc[212] += (double)v33_6_0;
+                const VT v33_7_0 = QCy * v33_2_0 + WQy * v33_2_1 + (VT)1.0 * oo2ze * v19_2_1 + (VT)1.0 * oo2e * (v33_0_0 - rho_e * v33_0_1);
+                acc[213] += (double)v33_7_0;
+                const VT v33_8_0 = QCy * v33_3_0 + WQy * v33_3_1 + (VT)1.0 * oo2ze * v19_3_1;
+                acc[214] += (double)v33_8_0;
+                const VT v33_9_0 = QCz * v33_3_0 + WQz * v33_3_1 + (VT)3.0 * oo2ze * v18_3_1 + (VT)1.0 * oo2e * (v33_0_0 - rho_e * v33_0_1);
+                acc[215] += (double)v33_9_0;
+                acc[216] += (double)v34_1_0;
+                acc[217] += (double)v34_2_0;
+                acc[218] += (double)v34_3_0;
+                const VT v34_4_0 = QCx * v34_1_0 + WQx * v34_1_1 + (VT)1.0 * oo2e * (v34_0_0 - rho_e * v34_0_1);
+                acc[219] += (double)v34_4_0;
+                const VT v34_5_0 = QCx * v34_2_0 + WQx * v34_2_1;
+                acc[220] += (double)v34_5_0;
+                const VT v34_6_0 = QCx * v34_3_0 + WQx * v34_3_1;
+                acc[221] += (double)v34_6_0;
+                const VT v34_7_0 = QCy * v34_2_0 + WQy * v34_2_1 + (VT)1.0 * oo2e * (v34_0_0 - rho_e * v34_0_1);
+                acc[222] += (double)v34_7_0;
+                const VT v34_8_0 = QCy * v34_3_0 + WQy * v34_3_1;
+                acc[223] += (double)v34_8_0;
+                const VT v34_9_0 = QCz * v34_3_0 + WQz * v34_3_1 + (VT)4.0 * oo2ze * v19_3_1 + (VT)1.0 * oo2e * (v34_0_0 - rho_e * v34_0_1);
+                acc[224] += (double)v34_9_0;
+            }
         }
     }
 }

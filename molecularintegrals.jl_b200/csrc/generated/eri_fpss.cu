@@ -25,13 +25,13 @@ __device__ __forceinline__ void vrr_fpss(const PairTab &P, const BoysTab &B, int
             const double r = rsqrt(bra.zeta + ket.zeta);
             const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
-            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[5];
             boys_fm<4>(T, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
-            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
             const VT WQx = (VT)(zz * PQx), WQy = (VT)(zz * PQy), WQz = (VT)(zz * PQz);
             const VT oo2z = (VT)bra.oo2z, oo2e = (VT)ket.oo2z, oo2ze = (VT)(0.5 * r2);
@@ -94,46 +94,74 @@ __device__ __forceinline__ void vrr_fpss(const PairTab &P, const BoysTab &B, int
             const VT v18_0_1 = PAz * v8_0_1 + WPz * v8_0_2 + (VT)1.0 * oo2z * (v2_0_1 - rho_z * v2_0_2);
             const VT v19_0_0 = PAz * v9_0_0 + WPz * v9_0_1 + (VT)2.0 * oo2z * (v3_0_0 - rho_z * v3_0_1);
             const VT v19_0_1 = PAz * v9_0_1 + WPz * v9_0_2 + (VT)2.0 * oo2z * (v3_0_1 - rho_z * v3_0_2);
-            const VT v20_0_0 = PAx * v10_0_0 + WPx * v10_0_1 + (VT)3.0 * oo2z * (v4_0_0 - rho_z * v4_0_1);
-            const VT v21_0_0 = PAx * v11_0_0 + WPx * v11_0_1 + (VT)2.0 * oo2z * (v5_0_0 - rho_z * v5_0_1);
-            const VT v22_0_0 = PAx * v12_0_0 + WPx * v12_0_1 + (VT)2.0 * oo2z * (v6_0_0 - rho_z * v6_0_1);
-            const VT v23_0_0 = PAx * v13_0_0 + WPx * v13_0_1 + (VT)1.0 * oo2z * (v7_0_0 - rho_z * v7_0_1);
-            const VT v24_0_0 = PAx * v15_0_0 + WPx * v15_0_1 + (VT)1.0 * oo2z * (v8_0_0 - rho_z * v8_0_1);
-            const VT v25_0_0 = PAx * v14_0_0 + WPx * v14_0_1 + (VT)1.0 * oo2z * (v9_0_0 - rho_z * v9_0_1);
-            const VT v26_0_0 = PAy * v13_0_0 + WPy * v13_0_1 + (VT)2.0 * oo2z * (v5_0_0 - rho_z * v5_0_1);
-            const VT v27_0_0 = PAy * v15_0_0 + WPy * v15_0_1 + (VT)1.0 * oo2z * (v6_0_0 - rho_z * v6_0_1);
-            const VT v28_0_0 = PAz * v15_0_0 + WPz * v15_0_1 + (VT)1.0 * oo2z * (v5_0_0 - rho_z * v5_0_1);
-            const VT v29_0_0 = PAz * v14_0_0 + WPz * v14_0_1 + (VT)2.0 * oo2z * (v6_0_0 - rho_z * v6_0_1);
-            const VT v30_0_0 = PAy * v16_0_0 + WPy * v16_0_1 + (VT)3.0 * oo2z * (v7_0_0 - rho_z * v7_0_1);
-            const VT v31_0_0 = PAy * v17_0_0 + WPy * v17_0_1 + (VT)2.0 * oo2z * (v8_0_0 - rho_z * v8_0_1);
-            const VT v32_0_0 = PAy * v18_0_0 + WPy * v18_0_1 + (VT)1.0 * oo2z * (v9_0_0 - rho_z * v9_0_1);
-            const VT v33_0_0 = PAz * v18_0_0 + WPz * v18_0_1 + (VT)2.0 * oo2z * (v8_0_0 - rho_z * v8_0_1);
-            const VT v34_0_0 = PAz * v19_0_0 + WPz * v19_0_1 + (VT)3.0 * oo2z * (v9_0_0 - rho_z * v9_0_1);
-            acc[0] += (double)v10_0_0;
-            acc[1] += (double)v11_0_0;
-            acc[2] += (double)v12_0_0;
-            acc[3] += (double)v13_0_0;
-            acc[4] += (double)v14_0_0;
-            acc[5] += (double)v15_0_0;
-            acc[6] += (double)v16_0_0;
-            acc[7] += (double)v17_0_0;
-            acc[8] += (double)v18_0_0;
-            acc[9] += (double)v19_0_0;
-            acc[10] += (double)v20_0_0;
-            acc[11] += (double)v21_0_0;
-            acc[12] += (double)v22_0_0;
-            acc[13] += (double)v23_0_0;
-            acc[14] += (double)v24_0_0;
-            acc[15] += (double)v25_0_0;
-            acc[16] += (double)v26_0_0;
-            acc[17] += (double)v27_0_0;
-            acc[18] += (double)v28_0_0;
-            acc[19] += (double)v29_0_0;
-            acc[20] += (double)v30_0_0;
-            acc[21] += (double)v31_0_0;
-            acc[22] += (double)v32_0_0;
-            acc[23] += (double)v33_0_0;
-            acc[24] += (double)v34_0_0;
+            if constexpr (sizeof(VT) == 8) {
+                acc[0] += (double)v10_0_0;
+                acc[1] += (double)v11_0_0;
+                acc[2] += (double)v12_0_0;
+                acc[3] += (double)v13_0_0;
+                acc[4] += (double)v14_0_0;
+                acc[5] += (double)v15_0_0;
+                acc[6] += (double)v16_0_0;
+                acc[7] += (double)v17_0_0;
+                acc[8] += (double)v18_0_0;
+                acc[9] += (double)v19_0_0;
+                acc[10] = fma(PAx, v10_0_0, fma(WPx, v10_0_1, fma(3.0 * oo2z, (v4_0_0 - rho_z * v4_0_1), acc[10])));
+                acc[11] = fma(PAx, v11_0_0, fma(WPx, v11_0_1, fma(2.0 * oo2z, (v5_0_0 - rho_z * v5_0_1), acc[11])));
+                acc[12] = fma(PAx, v12_0_0, fma(WPx, v12_0_1, fma(2.0 * oo2z, (v6_0_0 - rho_z * v6_0_1), acc[12])));
+                acc[13] = fma(PAx, v13_0_0, fma(WPx, v13_0_1, fma(1.0 * oo2z, (v7_0_0 - rho_z * v7_0_1), acc[13])));
+                acc[14] = fma(PAx, v15_0_0, fma(WPx, v15_0_1, fma(1.0 * oo2z, (v8_0_0 - rho_z * v8_0_1), acc[14])));
+                acc[15] = fma(PAx, v14_0_0, fma(WPx, v14_0_1, fma(1.0 * oo2z, (v9_0_0 - rho_z * v9_0_1), acc[15])));
+                acc[16] = fma(PAy, v13_0_0, fma(WPy, v13_0_1, fma(2.0 * oo2z, (v5_0_0 - rho_z * v5_0_1), acc[16])));
+                acc[17] = fma(PAy, v15_0_0, fma(WPy, v15_0_1, fma(1.0 * oo2z, (v6_0_0 - rho_z * v6_0_1), acc[17])));
+                acc[18] = fma(PAz, v15_0_0, fma(WPz, v15_0_1, fma(1.0 * oo2z, (v5_0_0 - rho_z * v5_0_1), acc[18])));
+                acc[19] = fma(PAz, v14_0_0, fma(WPz, v14_0_1, fma(2.0 * oo2z, (v6_0_0 - rho_z * v6_0_1), acc[19])));
+                acc[20] = fma(PAy, v16_0_0, fma(WPy, v16_0_1, fma(3.0 * oo2z, (v7_0_0 - rho_z * v7_0_1), acc[20])));
+                acc[21] = fma(PAy, v17_0_0, fma(WPy, v17_0_1, fma(2.0 * oo2z, (v8_0_0 - rho_z * v8_0_1), acc[21])));
+                acc[22] = fma(PAy, v18_0_0, fma(WPy, v18_0_1, fma(1.0 * oo2z, (v9_0_0 - rho_z * v9_0_1), acc[22])));
+                acc[23] = fma(PAz, v18_0_0, fma(WPz, v18_0_1, fma(2.0 * oo2z, (v8_0_0 - rho_z * v8_0_1), acc[23])));
+                acc[24] = fma(PAz, v19_0_0, fma(WPz, v19_0_1, fma(3.0 * oo2z, (v9_0_0 - rho_z * v9_0_1), acc[24])));
+            } else {
+                acc[0] += (double)v10_0_0;
+                acc[1] += (double)v11_0_0;
+                acc[2] += (double)v12_0_0;
+                acc[3] += (double)v13_0_0;
+                acc[4] += (double)v14_0_0;
+                acc[5] += (double)v15_0_0;
+                acc[6] += (double)v16_0_0;
+                acc[7] += (double)v17_0_0;
+                acc[8] += (double)v18_0_0;
+                acc[9] += (double)v19_0_0;
+                const VT v20_0_0 = PAx * v10_0_0 + WPx * v10_0_1 + (VT)3.0 * oo2z * (v4_0_0 - rho_z * v4_0_1);
+                acc[10] += (double)v20_0_0;
+                const VT v21_0_0 = PAx * v11_0_0 + WPx * v11_0_1 + (VT)2.0 * oo2z * (v5_0_0 - rho_z * v5_0_1);
+                acc[11] += (double)v21_0_0;
+                const VT v22_0_0 = PAx * v12_0_0 + WPx * v12_0_1 + (VT)2.0 * oo2z * (v6_0_0 - rho_z * v6_0_1);
+                acc[12] += (double)v22_0_0;
+                const VT v23_0_0 = PAx * v13_0_0 + WPx * v13_0_1 + (VT)1.0 * oo2z * (v7_0_0 - rho_z * v7_0_1);
+                acc[13] += (double)v23_0_0;
+                const VT v24_0_0 = PAx * v15_0_0 + WPx * v15_0_1 + (VT)1.0 * oo2z * (v8_0_0 - rho_z * v8_0_1);
+                acc[14] += (double)v24_0_0;
+                const VT v25_0_0 = PAx * v14_0_0 + WPx * v14_0_1 + (VT)1.0 * oo2z * (v9_0_0 - rho_z * v9_0_1);
+                acc[15] += (double)v25_0_0;
+                const VT v26_0_0 = PAy * v13_0_0 + WPy * v13_0_1 + (VT)2.0 * oo2z * (v5_0_0 - rho_z * v5_0_1);
+                acc[16] += (double)v26_0_0;
+                const VT v27_0_0 = PAy * v15_0_0 + WPy * v15_0_1 + (VT)1.0 * oo2z * (v6_0_0 - rho_z * v6_0_1);
+                acc[17] += (double)v27_0_0;
+                const VT v28_0_0 = PAz * v15_0_0 + WPz * v15_0_1 + (VT)1.0 * oo2z * (v5_0_0 - rho_z * v5_0_1);
+                acc[18] += (double)v28_0_0;
+                const VT v29_0_0 = PAz * v14_0_0 + WPz * v14_0_1 + (VT)2.0 * oo2z * (v6_0_0 - rho_z * v6_0_1);
+                acc[19] += (double)v29_0_0;
+                const VT v30_0_0 = PAy * v16_0_0 + WPy * v16_0_1 + (VT)3.0 * oo2z * (v7_0_0 - rho_z * v7_0_1);
+                acc[20] += (double)v30_0_0;
+                const VT v31_0_0 = PAy * v17_0_0 + WPy * v17_0_1 + (VT)2.0 * oo2z * (v8_0_0 - rho_z * v8_0_1);
+                acc[21] += (double)v31_0_0;
+                const VT v32_0_0 = PAy * v18_0_0 + WPy * v18_0_1 + (VT)1.0 * oo2z * (v9_0_0 - rho_z * v9_0_1);
+                acc[22] += (double)v32_0_0;
+                const VT v33_0_0 = PAz * v18_0_0 + WPz * v18_0_1 + (VT)2.0 * oo2z * (v8_0_0 - rho_z * v8_0_1);
+                acc[23] += (double)v33_0_0;
+                const VT v34_0_0 = PAz * v19_0_0 + WPz * v19_0_1 + (VT)3.0 * oo2z * (v9_0_0 - rho_z * v9_0_1);
+                acc[24] += (double)v34_0_0;
+            }
         }
     }
 }

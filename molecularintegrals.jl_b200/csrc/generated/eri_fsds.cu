@@ -25,13 +25,13 @@ __device__ __forceinline__ void vrr_fsds(const PairTab &P, const BoysTab &B, int
             const double r = rsqrt(bra.zeta + ket.zeta);
             const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
-            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[6];
             boys_fm<5>(T, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
-            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
             const VT WQx = (VT)(zz * PQx), WQy = (VT)(zz * PQy), WQz = (VT)(zz * PQz);
             const VT oo2z = (VT)bra.oo2z, oo2e = (VT)ket.oo2z, oo2ze = (VT)(0.5 * r2);
@@ -192,126 +192,189 @@ __device__ __forceinline__ void vrr_fsds(const PairTab &P, const BoysTab &B, int
             const VT v18_3_1 = QCz * v18_0_1 + WQz * v18_0_2 + (VT)2.0 * oo2ze * v8_0_2;
             const VT v19_3_0 = QCz * v19_0_0 + WQz * v19_0_1 + (VT)3.0 * oo2ze * v9_0_1;
             const VT v19_3_1 = QCz * v19_0_1 + WQz * v19_0_2 + (VT)3.0 * oo2ze * v9_0_2;
-            const VT v10_4_0 = QCx * v10_1_0 + WQx * v10_1_1 + (VT)3.0 * oo2ze * v4_1_1 + (VT)1.0 * oo2e * (v10_0_0 - rho_e * v10_0_1);
-            const VT v11_4_0 = QCx * v11_1_0 + WQx * v11_1_1 + (VT)2.0 * oo2ze * v5_1_1 + (VT)1.0 * oo2e * (v11_0_0 - rho_e * v11_0_1);
-            const VT v12_4_0 = QCx * v12_1_0 + WQx * v12_1_1 + (VT)2.0 * oo2ze * v6_1_1 + (VT)1.0 * oo2e * (v12_0_0 - rho_e * v12_0_1);
-            const VT v13_4_0 = QCx * v13_1_0 + WQx * v13_1_1 + (VT)1.0 * oo2ze * v7_1_1 + (VT)1.0 * oo2e * (v13_0_0 - rho_e * v13_0_1);
-            const VT v14_4_0 = QCx * v14_1_0 + WQx * v14_1_1 + (VT)1.0 * oo2ze * v9_1_1 + (VT)1.0 * oo2e * (v14_0_0 - rho_e * v14_0_1);
-            const VT v15_4_0 = QCx * v15_1_0 + WQx * v15_1_1 + (VT)1.0 * oo2ze * v8_1_1 + (VT)1.0 * oo2e * (v15_0_0 - rho_e * v15_0_1);
-            const VT v16_4_0 = QCx * v16_1_0 + WQx * v16_1_1 + (VT)1.0 * oo2e * (v16_0_0 - rho_e * v16_0_1);
-            const VT v17_4_0 = QCx * v17_1_0 + WQx * v17_1_1 + (VT)1.0 * oo2e * (v17_0_0 - rho_e * v17_0_1);
-            const VT v18_4_0 = QCx * v18_1_0 + WQx * v18_1_1 + (VT)1.0 * oo2e * (v18_0_0 - rho_e * v18_0_1);
-            const VT v19_4_0 = QCx * v19_1_0 + WQx * v19_1_1 + (VT)1.0 * oo2e * (v19_0_0 - rho_e * v19_0_1);
-            const VT v10_5_0 = QCx * v10_2_0 + WQx * v10_2_1 + (VT)3.0 * oo2ze * v4_2_1;
-            const VT v11_5_0 = QCx * v11_2_0 + WQx * v11_2_1 + (VT)2.0 * oo2ze * v5_2_1;
-            const VT v12_5_0 = QCx * v12_2_0 + WQx * v12_2_1 + (VT)2.0 * oo2ze * v6_2_1;
-            const VT v13_5_0 = QCx * v13_2_0 + WQx * v13_2_1 + (VT)1.0 * oo2ze * v7_2_1;
-            const VT v14_5_0 = QCx * v14_2_0 + WQx * v14_2_1 + (VT)1.0 * oo2ze * v9_2_1;
-            const VT v15_5_0 = QCx * v15_2_0 + WQx * v15_2_1 + (VT)1.0 * oo2ze * v8_2_1;
-            const VT v16_5_0 = QCx * v16_2_0 + WQx * v16_2_1;
-            const VT v17_5_0 = QCx * v17_2_0 + WQx * v17_2_1;
-            const VT v18_5_0 = QCx * v18_2_0 + WQx * v18_2_1;
-            const VT v19_5_0 = QCx * v19_2_0 + WQx * v19_2_1;
-            const VT v10_6_0 = QCx * v10_3_0 + WQx * v10_3_1 + (VT)3.0 * oo2ze * v4_3_1;
-            const VT v11_6_0 = QCx * v11_3_0 + WQx * v11_3_1 + (VT)2.0 * oo2ze * v5_3_1;
-            const VT v12_6_0 = QCx * v12_3_0 + WQx * v12_3_1 + (VT)2.0 * oo2ze * v6_3_1;
-            const VT v13_6_0 = QCx * v13_3_0 + WQx * v13_3_1 + (VT)1.0 * oo2ze * v7_3_1;
-            const VT v14_6_0 = QCx * v14_3_0 + WQx * v14_3_1 + (VT)1.0 * oo2ze * v9_3_1;
-            const VT v15_6_0 = QCx * v15_3_0 + WQx * v15_3_1 + (VT)1.0 * oo2ze * v8_3_1;
-            const VT v16_6_0 = QCx * v16_3_0 + WQx * v16_3_1;
-            const VT v17_6_0 = QCx * v17_3_0 + WQx * v17_3_1;
-            const VT v18_6_0 = QCx * v18_3_0 + WQx * v18_3_1;
-            const VT v19_6_0 = QCx * v19_3_0 + WQx * v19_3_1;
-            const VT v10_7_0 = QCy * v10_2_0 + WQy * v10_2_1 + (VT)1.0 * oo2e * (v10_0_0 - rho_e * v10_0_1);
-            const VT v11_7_0 = QCy * v11_2_0 + WQy * v11_2_1 + (VT)1.0 * oo2ze * v4_2_1 + (VT)1.0 * oo2e * (v11_0_0 - rho_e * v11_0_1);
-            const VT v12_7_0 = QCy * v12_2_0 + WQy * v12_2_1 + (VT)1.0 * oo2e * (v12_0_0 - rho_e * v12_0_1);
-            const VT v13_7_0 = QCy * v13_2_0 + WQy * v13_2_1 + (VT)2.0 * oo2ze * v5_2_1 + (VT)1.0 * oo2e * (v13_0_0 - rho_e * v13_0_1);
-            const VT v14_7_0 = QCy * v14_2_0 + WQy * v14_2_1 + (VT)1.0 * oo2e * (v14_0_0 - rho_e * v14_0_1);
-            const VT v15_7_0 = QCy * v15_2_0 + WQy * v15_2_1 + (VT)1.0 * oo2ze * v6_2_1 + (VT)1.0 * oo2e * (v15_0_0 - rho_e * v15_0_1);
-            const VT v16_7_0 = QCy * v16_2_0 + WQy * v16_2_1 + (VT)3.0 * oo2ze * v7_2_1 + (VT)1.0 * oo2e * (v16_0_0 - rho_e * v16_0_1);
-            const VT v17_7_0 = QCy * v17_2_0 + WQy * v17_2_1 + (VT)2.0 * oo2ze * v8_2_1 + (VT)1.0 * oo2e * (v17_0_0 - rho_e * v17_0_1);
-            const VT v18_7_0 = QCy * v18_2_0 + WQy * v18_2_1 + (VT)1.0 * oo2ze * v9_2_1 + (VT)1.0 * oo2e * (v18_0_0 - rho_e * v18_0_1);
-            const VT v19_7_0 = QCy * v19_2_0 + WQy * v19_2_1 + (VT)1.0 * oo2e * (v19_0_0 - rho_e * v19_0_1);
-            const VT v10_8_0 = QCy * v10_3_0 + WQy * v10_3_1;
-            const VT v11_8_0 = QCy * v11_3_0 + WQy * v11_3_1 + (VT)1.0 * oo2ze * v4_3_1;
-            const VT v12_8_0 = QCy * v12_3_0 + WQy * v12_3_1;
-            const VT v13_8_0 = QCy * v13_3_0 + WQy * v13_3_1 + (VT)2.0 * oo2ze * v5_3_1;
-            const VT v14_8_0 = QCy * v14_3_0 + WQy * v14_3_1;
-            const VT v15_8_0 = QCy * v15_3_0 + WQy * v15_3_1 + (VT)1.0 * oo2ze * v6_3_1;
-            const VT v16_8_0 = QCy * v16_3_0 + WQy * v16_3_1 + (VT)3.0 * oo2ze * v7_3_1;
-            const VT v17_8_0 = QCy * v17_3_0 + WQy * v17_3_1 + (VT)2.0 * oo2ze * v8_3_1;
-            const VT v18_8_0 = QCy * v18_3_0 + WQy * v18_3_1 + (VT)1.0 * oo2ze * v9_3_1;
-            const VT v19_8_0 = QCy * v19_3_0 + WQy * v19_3_1;
-            const VT v10_9_0 = QCz * v10_3_0 + WQz * v10_3_1 + (VT)1.0 * oo2e * (v10_0_0 - rho_e * v10_0_1);
-            const VT v11_9_0 = QCz * v11_3_0 + WQz * v11_3_1 + (VT)1.0 * oo2e * (v11_0_0 - rho_e * v11_0_1);
-            const VT v12_9_0 = QCz * v12_3_0 + WQz * v12_3_1 + (VT)1.0 * oo2ze * v4_3_1 + (VT)1.0 * oo2e * (v12_0_0 - rho_e * v12_0_1);
-            const VT v13_9_0 = QCz * v13_3_0 + WQz * v13_3_1 + (VT)1.0 * oo2e * (v13_0_0 - rho_e * v13_0_1);
-            const VT v14_9_0 = QCz * v14_3_0 + WQz * v14_3_1 + (VT)2.0 * oo2ze * v6_3_1 + (VT)1.0 * oo2e * (v14_0_0 - rho_e * v14_0_1);
-            const VT v15_9_0 = QCz * v15_3_0 + WQz * v15_3_1 + (VT)1.0 * oo2ze * v5_3_1 + (VT)1.0 * oo2e * (v15_0_0 - rho_e * v15_0_1);
-            const VT v16_9_0 = QCz * v16_3_0 + WQz * v16_3_1 + (VT)1.0 * oo2e * (v16_0_0 - rho_e * v16_0_1);
-            const VT v17_9_0 = QCz * v17_3_0 + WQz * v17_3_1 + (VT)1.0 * oo2ze * v7_3_1 + (VT)1.0 * oo2e * (v17_0_0 - rho_e * v17_0_1);
-            const VT v18_9_0 = QCz * v18_3_0 + WQz * v18_3_1 + (VT)2.0 * oo2ze * v8_3_1 + (VT)1.0 * oo2e * (v18_0_0 - rho_e * v18_0_1);
-            const VT v19_9_0 = QCz * v19_3_0 + WQz * v19_3_1 + (VT)3.0 * oo2ze * v9_3_1 + (VT)1.0 * oo2e * (v19_0_0 - rho_e * v19_0_1);
-            acc[0] += (double)v10_4_0;
-            acc[1] += (double)v10_5_0;
-            acc[2] += (double)v10_6_0;
-            acc[3] += (double)v10_7_0;
-            acc[4] += (double)v10_8_0;
-            acc[5] += (double)v10_9_0;
-            acc[6] += (double)v11_4_0;
-            acc[7] += (double)v11_5_0;
-            acc[8] += (double)v11_6_0;
-            acc[9] += (double)v11_7_0;
-            acc[10] += (double)v11_8_0;
-            acc[11] += (double)v11_9_0;
-            acc[12] += (double)v12_4_0;
-            acc[13] += (double)v12_5_0;
-            acc[14] += (double)v12_6_0;
-            acc[15] += (double)v12_7_0;
-            acc[16] += (double)v12_8_0;
-            acc[17] += (double)v12_9_0;
-            acc[18] += (double)v13_4_0;
-            acc[19] += (double)v13_5_0;
-            acc[20] += (double)v13_6_0;
-            acc[21] += (double)v13_7_0;
-            acc[22] += (double)v13_8_0;
-            acc[23] += (double)v13_9_0;
-            acc[24] += (double)v14_4_0;
-            acc[25] += (double)v14_5_0;
-            acc[26] += (double)v14_6_0;
-            acc[27] += (double)v14_7_0;
-            acc[28] += (double)v14_8_0;
-            acc[29] += (double)v14_9_0;
-            acc[30] += (double)v15_4_0;
-            acc[31] += (double)v15_5_0;
-            acc[32] += (double)v15_6_0;
-            acc[33] += (double)v15_7_0;
-            acc[34] += (double)v15_8_0;
-            acc[35] += (double)v15_9_0;
-            acc[36] += (double)v16_4_0;
-            acc[37] += (double)v16_5_0;
-            acc[38] += (double)v16_6_0;
-            acc[39] += (double)v16_7_0;
-            acc[40] += (double)v16_8_0;
-            acc[41] += (double)v16_9_0;
-            acc[42] += (double)v17_4_0;
-            acc[43] += (double)v17_5_0;
-            acc[44] += (double)v17_6_0;
-            acc[45] += (double)v17_7_0;
-            acc[46] += (double)v17_8_0;
-            acc[47] += (double)v17_9_0;
-            acc[48] += (double)v18_4_0;
-            acc[49] += (double)v18_5_0;
-            acc[50] += (double)v18_6_0;
-            acc[51] += (double)v18_7_0;
-            acc[52] += (double)v18_8_0;
-            acc[53] += (double)v18_9_0;
-            acc[54] += (double)v19_4_0;
-            acc[55] += (double)v19_5_0;
-            acc[56] += (double)v19_6_0;
-            acc[57] += (double)v19_7_0;
-            acc[58] += (double)v19_8_0;
-            acc[59] += (double)v19_9_0;
+            if constexpr (sizeof(VT) == 8) {
+                acc[0] = fma(QCx, v10_1_0, fma(WQx, v10_1_1, fma(3.0 * oo2ze, v4_1_1, fma(1.0 * oo2e, (v10_0_0 - rho_e * v10_0_1), acc[0]))));
+                acc[1] = fma(QCx, v10_2_0, fma(WQx, v10_2_1, fma(3.0 * oo2ze, v4_2_1, acc[1])));
+                acc[2] = fma(QCx, v10_3_0, fma(WQx, v10_3_1, fma(3.0 * oo2ze, v4_3_1, acc[2])));
+                acc[3] = fma(QCy, v10_2_0, fma(WQy, v10_2_1, fma(1.0 * oo2e, (v10_0_0 - rho_e * v10_0_1), acc[3])));
+                acc[4] = fma(QCy, v10_3_0, fma(WQy, v10_3_1, acc[4]));
+                acc[5] = fma(QCz, v10_3_0, fma(WQz, v10_3_1, fma(1.0 * oo2e, (v10_0_0 - rho_e * v10_0_1), acc[5])));
+                acc[6] = fma(QCx, v11_1_0, fma(WQx, v11_1_1, fma(2.0 * oo2ze, v5_1_1, fma(1.0 * oo2e, (v11_0_0 - rho_e * v11_0_1), acc[6]))));
+                acc[7] = fma(QCx, v11_2_0, fma(WQx, v11_2_1, fma(2.0 * oo2ze, v5_2_1, acc[7])));
+                acc[8] = fma(QCx, v11_3_0, fma(WQx, v11_3_1, fma(2.0 * oo2ze, v5_3_1, acc[8])));
+                acc[9] = fma(QCy, v11_2_0, fma(WQy, v11_2_1, fma(1.0 * oo2ze, v4_2_1, fma(1.0 * oo2e, (v11_0_0 - rho_e * v11_0_1), acc[9]))));
+                acc[10] = fma(QCy, v11_3_0, fma(WQy, v11_3_1, fma(1.0 * oo2ze, v4_3_1, acc[10])));
+                acc[11] = fma(QCz, v11_3_0, fma(WQz, v11_3_1, fma(1.0 * oo2e, (v11_0_0 - rho_e * v11_0_1), acc[11])));
+                acc[12] = fma(QCx, v12_1_0, fma(WQx, v12_1_1, fma(2.0 * oo2ze, v6_1_1, fma(1.0 * oo2e, (v12_0_0 - rho_e * v12_0_1), acc[12]))));
+                acc[13] = fma(QCx, v12_2_0, fma(WQx, v12_2_1, fma(2.0 * oo2ze, v6_2_1, acc[13])));
+                acc[14] = fma(QCx, v12_3_0, fma(WQx, v12_3_1, fma(2.0 * oo2ze, v6_3_1, acc[14])));
+                acc[15] = fma(QCy, v12_2_0, fma(WQy, v12_2_1, fma(1.0 * oo2e, (v12_0_0 - rho_e * v12_0_1), acc[15])));
+                acc[16] = fma(QCy, v12_3_0, fma(WQy, v12_3_1, acc[16]));
+                acc[17] = fma(QCz, v12_3_0, fma(WQz, v12_3_1, fma(1.0 * oo2ze, v4_3_1, fma(1.0 * oo2e, (v12_0_0 - rho_e * v12_0_1), acc[17]))));
+                acc[18] = fma(QCx, v13_1_0, fma(WQx, v13_1_1, fma(1.0 * oo2ze, v7_1_1, fma(1.0 * oo2e, (v13_0_0 - rho_e * v13_0_1), acc[18]))));
+                acc[19] = fma(QCx, v13_2_0, fma(WQx, v13_2_1, fma(1.0 * oo2ze, v7_2_1, acc[19])));
+                acc[20] = fma(QCx, v13_3_0, fma(WQx, v13_3_1, fma(1.0 * oo2ze, v7_3_1, acc[20])));
+                acc[21] = fma(QCy, v13_2_0, fma(WQy, v13_2_1, fma(2.0 * oo2ze, v5_2_1, fma(1.0 * oo2e, (v13_0_0 - rho_e * v13_0_1), acc[21]))));
+                acc[22] = fma(QCy, v13_3_0, fma(WQy, v13_3_1, fma(2.0 * oo2ze, v5_3_1, acc[22])));
+                acc[23] = fma(QCz, v13_3_0, fma(WQz, v13_3_1, fma(1.0 * oo2e, (v13_0_0 - rho_e * v13_0_1), acc[23])));
+                acc[24] = fma(QCx, v14_1_0, fma(WQx, v14_1_1, fma(1.0 * oo2ze, v9_1_1, fma(1.0 * oo2e, (v14_0_0 - rho_e * v14_0_1), acc[24]))));
+                acc[25] = fma(QCx, v14_2_0, fma(WQx, v14_2_1, fma(1.0 * oo2ze, v9_2_1, acc[25])));
+                acc[26] = fma(QCx, v14_3_0, fma(WQx, v14_3_1, fma(1.0 * oo2ze, v9_3_1, acc[26])));
+                acc[27] = fma(QCy, v14_2_0, fma(WQy, v14_2_1, fma(1.0 * oo2e, (v14_0_0 - rho_e * v14_0_1), acc[27])));
+                acc[28] = fma(QCy, v14_3_0, fma(WQy, v14_3_1, acc[28]));
+                acc[29] = fma(QCz, v14_3_0, fma(WQz, v14_3_1, fma(2.0 * oo2ze, v6_3_1, fma(1.0 * oo2e, (v14_0_0 - rho_e * v14_0_1), acc[29]))));
+                acc[30] = fma(QCx, v15_1_0, fma(WQx, v15_1_1, fma(1.0 * oo2ze, v8_1_1, fma(1.0 * oo2e, (v15_0_0 - rho_e * v15_0_1), acc[30]))));
+                acc[31] = fma(QCx, v15_2_0, fma(WQx, v15_2_1, fma(1.0 * oo2ze, v8_2_1, acc[31])));
+                acc[32] = fma(QCx, v15_3_0, fma(WQx, v15_3_1, fma(1.0 * oo2ze, v8_3_1, acc[32])));
+                acc[33] = fma(QCy, v15_2_0, fma(WQy, v15_2_1, fma(1.0 * oo2ze, v6_2_1, fma(1.0 * oo2e, (v15_0_0 - rho_e * v15_0_1), acc[33]))));
+                acc[34] = fma(QCy, v15_3_0, fma(WQy, v15_3_1, fma(1.0 * oo2ze, v6_3_1, acc[34])));
+                acc[35] = fma(QCz, v15_3_0, fma(WQz, v15_3_1, fma(1.0 * oo2ze, v5_3_1, fma(1.0 * oo2e, (v15_0_0 - rho_e * v15_0_1), acc[35]))));
+                acc[36] = fma(QCx, v16_1_0, fma(WQx, v16_1_1, fma(1.0 * oo2e, (v16_0_0 - rho_e * v16_0_1), acc[36])));
+                acc[37] = fma(QCx, v16_2_0, fma(WQx, v16_2_1, acc[37]));
+                acc[38] = fma(QCx, v16_3_0, fma(WQx, v16_3_1, acc[38]));
+                acc[39] = fma(QCy, v16_2_0, fma(WQy, v16_2_1, fma(3.0 * oo2ze, v7_2_1, fma(1.0 * oo2e, (v16_0_0 - rho_e * v16_0_1), acc[39]))));
+                acc[40] = fma(QCy, v16_3_0, fma(WQy, v16_3_1, fma(3.0 * oo2ze, v7_3_1, acc[40])));
+                acc[41] = fma(QCz, v16_3_0, fma(WQz, v16_3_1, fma(1.0 * oo2e, (v16_0_0 - rho_e * v16_0_1), acc[41])));
+                acc[42] = fma(QCx, v17_1_0, fma(WQx, v17_1_1, fma(1.0 * oo2e, (v17_0_0 - rho_e * v17_0_1), acc[42])));
+                acc[43] = fma(QCx, v17_2_0, fma(WQx, v17_2_1, acc[43]));
+                acc[44] = fma(QCx, v17_3_0, fma(WQx, v17_3_1, acc[44]));
+                acc[45] = fma(QCy, v17_2_0, fma(WQy, v17_2_1, fma(2.0 * oo2ze, v8_2_1, fma(1.0 * oo2e, (v17_0_0 - rho_e * v17_0_1), acc[45]))));
+                acc[46] = fma(QCy, v17_3_0, fma(WQy, v17_3_1, fma(2.0 * oo2ze, v8_3_1, acc[46])));
+                acc[47] = fma(QCz, v17_3_0, fma(WQz, v17_3_1, fma(1.0 * oo2ze, v7_3_1, fma(1.0 * oo2e, (v17_0_0 - rho_e * v17_0_1), acc[47]))));
+                acc[48] = fma(QCx, v18_1_0, fma(WQx, v18_1_1, fma(1.0 * oo2e, (v18_0_0 - rho_e * v18_0_1), acc[48])));
+                acc[49] = fma(QCx, v18_2_0, fma(WQx, v18_2_1, acc[49]));
+                acc[50] = fma(QCx, v18_3_0, fma(WQx, v18_3_1, acc[50]));
+                acc[51] = fma(QCy, v18_2_0, fma(WQy, v18_2_1, fma(1.0 * oo2ze, v9_2_1, fma(1.0 * oo2e, (v18_0_0 - rho_e * v18_0_1), acc[51]))));
+                acc[52] = fma(QCy, v18_3_0, fma(WQy, v18_3_1, fma(1.0 * oo2ze, v9_3_1, acc[52])));
+                acc[53] = fma(QCz, v18_3_0, fma(WQz, v18_3_1, fma(2.0 * oo2ze, v8_3_1, fma(1.0 * oo2e, (v18_0_0 - rho_e * v18_0_1), acc[53]))));
+                acc[54] = fma(QCx, v19_1_0, fma(WQx, v19_1_1, fma(1.0 * oo2e, (v19_0_0 - rho_e * v19_0_1), acc[54])));
+                acc[55] = fma(QCx, v19_2_0, fma(WQx, v19_2_1, acc[55]));
+                acc[56] = fma(QCx, v19_3_0, fma(WQx, v19_3_1, acc[56]));
+                acc[57] = fma(QCy, v19_2_0, fma(WQy, v19_2_1, fma(1.0 * oo2e, (v19_0_0 - rho_e * v19_0_1), acc[57])));
+                acc[58] = fma(QCy, v19_3_0, fma(WQy, v19_3_1, acc[58]));
+                acc[59] = fma(QCz, v19_3_0, fma(WQz, v19_3_1, fma(3.0 * oo2ze, v9_3_1, fma(1.0 * oo2e, (v19_0_0 - rho_e * v19_0_1), acc[59]))));
+            } else {
+                const VT v10_4_0 = QCx * v10_1_0 + WQx * v10_1_1 + (VT)3.0 * oo2ze * v4_1_1 + (VT)1.0 * oo2e * (v10_0_0 - rho_e * v10_0_1);
+                acc[0] += (double)v10_4_0;
+                const VT v10_5_0 = QCx * v10_2_0 + WQx * v10_2_1 + (VT)3.0 * oo2ze * v4_2_1;
+                acc[1] += (double)v10_5_0;
+                const VT v10_6_0 = QCx * v10_3_0 + WQx * v10_3_1 + (VT)3.0 * oo2ze * v4_3_1;
+                acc[2] += (double)v10_6_0;
+                const VT v10_7_0 = QCy * v10_2_0 + WQy * v10_2_1 + (VT)1.0 * oo2e * (v10_0_0 - rho_e * v10_0_1);
+                acc[3] += (double)v10_7_0;
+                const VT v10_8_0 = QCy * v10_3_0 + WQy * v10_3_1;
+                acc[4] += (double)v10_8_0;
+                const VT v10_9_0 = QCz * v10_3_0 + WQz * v10_3_1 + (VT)1.0 * oo2e * (v10_0_0 - rho_e * v10_0_1);
+                acc[5] += (double)v10_9_0;
+                const VT v11_4_0 = QCx * v11_1_0 + WQx * v11_1_1 + (VT)2.0 * oo2ze * v5_1_1 + (VT)1.0 * oo2e * (v11_0_0 - rho_e * v11_0_1);
+                acc[6] += (double)v11_4_0;
+                const VT v11_5_0 = QCx * v11_2_0 + WQx * v11_2_1 + (VT)2.0 * oo2ze * v5_2_1;
+                acc[7] += (double)v11_5_0;
+                const VT v11_6_0 = QCx * v11_3_0 + WQx * v11_3_1 + (VT)2.0 * oo2ze * v5_3_1;
+                acc[8] += (double)v11_6_0;
+                const VT v11_7_0 = QCy * v11_2_0 + WQy * v11_2_1 + (VT)1.0 * oo2ze * v4_2_1 + (VT)1.0 * oo2e * (v11_0_0 - rho_e * v11_0_1);
+                acc[9] += (double)v11_7_0;
+                const VT v11_8_0 = QCy * v11_3_0 + WQy * v11_3_1 + (VT)1.0 * oo2ze * v4_3_1;
+                acc[10] += (double)v11_8_0;
+                const VT v11_9_0 = QCz * v11_3_0 + WQz * v11_3_1 + (VT)1.0 * oo2e * (v11_0_0 - rho_e * v11_0_1);
+                acc[11] += (double)v11_9_0;
+                const VT v12_4_0 = QCx * v12_1_0 + WQx * v12_1_1 + (VT)2.0 * oo2ze * v6_1_1 + (VT)1.0 * oo2e * (v12_0_0 - rho_e * v12_0_1);
+                acc[12] += (double)v12_4_0;
+                const VT v12_5_0 = QCx * v12_2_0 + WQx * v12_2_1 + (VT)2.0 * oo2ze * v6_2_1;
+                acc[13] += (double)v12_5_0;
+                const VT v12_6_0 = QCx * v12_3_0 + WQx * v12_3_1 + (VT)2.0 * oo2ze * v6_3_1;
+                acc[14] += (double)v12_6_0;
+                const VT v12_7_0 = QCy * v12_2_0 + WQy * v12_2_1 + (VT)1.0 * oo2e * (v12_0_0 - rho_e * v12_0_1);
+                acc[15] += (double)v12_7_0;
+                const VT v12_8_0 = QCy * v12_3_0 + WQy * v12_3_1;
+                acc[16] += (double)v12_8_0;
+                const VT v12_9_0 = QCz * v12_3_0 + WQz * v12_3_1 + (VT)1.0 * oo2ze * v4_3_1 + (VT)1.0 * oo2e * (v12_0_0 - rho_e * v12_0_1);
+                acc[17] += (double)v12_9_0;
+                const VT v13_4_0 = QCx * v13_1_0 + WQx * v13_1_1 + (VT)1.0 * oo2ze * v7_1_1 + (VT)1.0 * oo2e * (v13_0_0 - rho_e * v13_0_1);
+                acc[18] += (double)v13_4_0;
+                const VT v13_5_0 = QCx * v13_2_0 + WQx * v13_2_1 + (VT)1.0 * oo2ze * v7_2_1;
+                acc[19] += (double)v13_5_0;
+                const VT v13_6_0 = QCx * v13_3_0 + WQx * v13_3_1 + (VT)1.0 * oo2ze * v7_3_1;
+                acc[20] += (double)v13_6_0;
+                const VT v13_7_0 = QCy * v13_2_0 + WQy * v13_2_1 + (VT)2.0 * oo2ze * v5_2_1 + (VT)1.0 * oo2e * (v13_0_0 - rho_e * v13_0_1);
+                acc[21] += (double)v13_7_0;
+                const VT v13_8_0 = QCy * v13_3_0 + WQy * v13_3_1 + (VT)2.0 * oo2ze * v5_3_1;
+                acc[22] += (double)v13_8_0;
+                const VT v13_9_0 = QCz * v13_3_0 + WQz * v13_3_1 + (VT)1.0 * oo2e * (v13_0_0 - rho_e * v13_0_1);
+                acc[23] += (double)v13_9_0;
+                const VT v14_4_0 = QCx * v14_1_0 + WQx * v14_1_1 + (VT)1.0 * oo2ze * v9_1_1 + (VT)1.0 * oo2e * (v14_0_0 - rho_e * v14_0_1);
+                acc[24] += (double)v14_4_0;
+                const VT v14_5_0 = QCx * v14_2_0 + WQx * v14_2_1 + (VT)1.0 * oo2ze * v9_2_1;
+                acc[25] += (double)v14_5_0;
+                const VT v14_6_0 = QCx * v14_3_0 + WQx * v14_3_1 + (VT)1.0 * oo2ze * v9_3_1;
+                acc[26] += (double)v14_6_0;
+                const VT v14_7_0 = QCy * v14_2_0 + WQy * v14_2_1 + (VT)1.0 * oo2e * (v14_0_0 - rho_e * v14_0_1);
+                acc[27] += (double)v14_7_0;
+                const VT v14_8_0 = QCy * v14_3_0 + WQy * v14_3_1;
+                acc[28] += (double)v14_8_0;
+                const VT v14_9_0 = QCz * v14_3_0 + WQz * v14_3_1 + (VT)2.0 * oo2ze * v6_3_1 + (VT)1.0 * oo2e * (v14_0_0 - rho_e * v14_0_1);
+                acc[29] += (double)v14_9_0;
+                const VT v15_4_0 = QCx * v15_1_0 + WQx * v15_1_1 + (VT)1.0 * oo2ze * v8_1_1 + (VT)1.0 * oo2e * (v15_0_0 - rho_e * v15_0_1);
+                acc[30] += (double)v15_4_0;
+                const VT v15_5_0 = QCx * v15_2_0 + WQx * v15_2_1 + (VT)1.0 * oo2ze * v8_2_1;
+                acc[31] += (double)v15_5_0;
+                const VT v15_6_0 = QCx * v15_3_0 + WQx * v15_3_1 + (VT)1.0 * oo2ze * v8_3_1;
+                acc[32] += (double)v15_6_0;
+                const VT v15_7_0 = QCy * v15_2_0 + WQy * v15_2_1 + (VT)1.0 * oo2ze * v6_2_1 + (VT)1.0 * oo2e * (v15_0_0 - rho_e * v15_0_1);
+                acc[33] += (double)v15_7_0;
+                const VT v15_8_0 = QCy * v15_3_0 + WQy * v15_3_1 + (VT)1.0 * oo2ze * v6_3_1;
+                acc[34] += (double)v15_8_0;
+                const VT v15_9_0 = QCz * v15_3_0 + WQz * v15_3_1 + (VT)1.0 * oo2ze * v5_3_1 + (VT)1.0 * oo2e * (v15_0_0 - rho_e * v15_0_1);
+                acc[35] += (double)v15_9_0;
+                const VT v16_4_0 = QCx * v16_1_0 + WQx * v16_1_1 + (VT)1.0 * oo2e * (v16_0_0 - rho_e * v16_0_1);
+                acc[36] += (double)v16_4_0;
+                const VT v16_5_0 = QCx * v16_2_0 + WQx * v16_2_1;
+                acc[37] += (double)v16_5_0;
+                const VT v16_6_0 = QCx * v16_3_0 + WQx * v16_3_1;
+                acc[38] += (double)v16_6_0;
+                const VT v16_7_0 = QCy * v16_2_0 + WQy * v16_2_1 + (VT)3.0 * oo2ze * v7_2_1 + (VT)1.0 * oo2e * (v16_0_0 - rho_e * v16_0_1);
+                acc[39] += (double)v16_7_0;
+                const VT v16_8_0 = QCy * v16_3_0 + WQy * v16_3_1 + (VT)3.0 * oo2ze * v7_3_1;
+                acc[40] += (double)v16_8_0;
+                const VT v16_9_0 = QCz * v16_3_0 + WQz * v16_3_1 + (VT)1.0 * oo2e * (v16_0_0 - rho_e * v16_0_1);
+                acc[41] += (double)v16_9_0;
+                const VT v17_4_0 = QCx * v17_1_0 + WQx * v17_1_1 + (VT)1.0 * oo2e * (v17_0_0 - rho_e * v17_0_1);
+                acc[42] += (double)v17_4_0;
+                const VT v17_5_0 = QCx * v17_2_0 + WQx * v17_2_1;
+                acc[43] += (double)v17_5_0;
+                const VT v17_6_0 = QCx * v17_3_0 + WQx * v17_3_1;
+                acc[44] += (double)v17_6_0;
+                const VT v17_7_0 = QCy * v17_2_0 + WQy * v17_2_1 + (VT)2.0 * oo2ze * v8_2_1 + (VT)1.0 * oo2e * (v17_0_0 - rho_e * v17_0_1);
+                acc[45] += (double)v17_7_0;
+                const VT v17_8_0 = QCy * v17_3_0 + WQy * v17_3_1 + (VT)2.0 * oo2ze * v8_3_1;
+                acc[46] += (double)v17_8_0;
+                const VT v17_9_0 = QCz * v17_3_0 + WQz * v17_3_1 + (VT)1.0 * oo2ze * v7_3_1 + (VT)1.0 * oo2e * (v17_0_0 - rho_e * v17_0_1);
+                acc[47] += (double)v17_9_0;
+                const VT v18_4_0 = QCx * v18_1_0 + WQx * v18_1_1 + (VT)1.0 * oo2e * (v18_0_0 - rho_e * v18_0_1);
+                acc[48] += (double)v18_4_0;
+                const VT v18_5_0 = QCx * v18_2_0 + WQx * v18_2_1;
+                acc[49] += (double)v18_5_0;
+                const VT v18_6_0 = QCx * v18_3_0 + WQx * v18_3_1;
+                acc[50] += (double)v18_6_0;
+                const VT v18_7_0 = QCy * v18_2_0 + WQy * v18_2_1 + (VT)1.0 * oo2ze * v9_2_1 + (VT)1.0 * oo2e * (v18_0_0 - rho_e * v18_0_1);
+                acc[51] += (double)v18_7_0;
+                const VT v18_8_0 = QCy * v18_3_0 + WQy * v18_3_1 + (VT)1.0 * oo2ze * v9_3_1;
+                acc[52] += (double)v18_8_0;
+                const VT v18_9_0 = QCz * v18_3_0 + WQz * v18_3_1 + (VT)2.0 * oo2ze * v8_3_1 + (VT)1.0 * oo2e * (v18_0_0 - rho_e * v18_0_1);
+                acc[53] += (double)v18_9_0;
+                const VT v19_4_0 = QCx * v19_1_0 + WQx * v19_1_1 + (VT)1.0 * oo2e * (v19_0_0 - rho_e * v19_0_1);
+                acc[54] += (double)v19_4_0;
+                const VT v19_5_0 = QCx * v19_2_0 + WQx * v19_2_1;
+                acc[55] += (double)v19_5_0;
+                const VT v19_6_0 = QCx * v19_3_0 + WQx * v19_3_1;
+                acc[56] += (double)v19_6_0;
+                const VT v19_7_0 = QCy * v19_2_0 + WQy * v19_2_1 + (VT)1.0 * oo2e * (v19_0_0 - rho_e * v19_0_1);
+                acc[57] += (double)v19_7_0;
+                const VT v19_8_0 = QCy * v19_3_0 + WQy * v19_3_1;
+                acc[58] += (double)v19_8_0;
+                const VT v19_9_0 = QCz * v19_3_0 + WQz * v19_3_1 + (VT)3.0 * oo2ze * v9_3_1 + (VT)1.0 * oo2e * (v19_0_0 - rho_e * v19_0_1);
+                acc[59] += (double)v19_9_0;
+            }
         }
     }
 }

@@ -25,13 +25,13 @@ __device__ __forceinline__ void vrr_pppp(const PairTab &P, const BoysTab &B, int
             const double r = rsqrt(bra.zeta + ket.zeta);
             const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
-            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[5];
             boys_fm<4>(T, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
-            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
             const VT WQx = (VT)(zz * PQx), WQy = (VT)(zz * PQy), WQz = (VT)(zz * PQz);
             const VT oo2z = (VT)bra.oo2z, oo2e = (VT)ket.oo2z, oo2ze = (VT)(0.5 * r2);
@@ -131,141 +131,225 @@ __device__ __forceinline__ void vrr_pppp(const PairTab &P, const BoysTab &B, int
             const VT v8_3_1 = QCz * v8_0_1 + WQz * v8_0_2 + (VT)1.0 * oo2ze * v2_0_2;
             const VT v9_3_0 = QCz * v9_0_0 + WQz * v9_0_1 + (VT)2.0 * oo2ze * v3_0_1;
             const VT v9_3_1 = QCz * v9_0_1 + WQz * v9_0_2 + (VT)2.0 * oo2ze * v3_0_2;
-            const VT v1_4_0 = QCx * v1_1_0 + WQx * v1_1_1 + (VT)1.0 * oo2ze * v0_1_1 + (VT)1.0 * oo2e * (v1_0_0 - rho_e * v1_0_1);
-            const VT v2_4_0 = QCx * v2_1_0 + WQx * v2_1_1 + (VT)1.0 * oo2e * (v2_0_0 - rho_e * v2_0_1);
-            const VT v3_4_0 = QCx * v3_1_0 + WQx * v3_1_1 + (VT)1.0 * oo2e * (v3_0_0 - rho_e * v3_0_1);
-            const VT v4_4_0 = QCx * v4_1_0 + WQx * v4_1_1 + (VT)2.0 * oo2ze * v1_1_1 + (VT)1.0 * oo2e * (v4_0_0 - rho_e * v4_0_1);
-            const VT v5_4_0 = QCx * v5_1_0 + WQx * v5_1_1 + (VT)1.0 * oo2ze * v2_1_1 + (VT)1.0 * oo2e * (v5_0_0 - rho_e * v5_0_1);
-            const VT v6_4_0 = QCx * v6_1_0 + WQx * v6_1_1 + (VT)1.0 * oo2ze * v3_1_1 + (VT)1.0 * oo2e * (v6_0_0 - rho_e * v6_0_1);
-            const VT v7_4_0 = QCx * v7_1_0 + WQx * v7_1_1 + (VT)1.0 * oo2e * (v7_0_0 - rho_e * v7_0_1);
-            const VT v8_4_0 = QCx * v8_1_0 + WQx * v8_1_1 + (VT)1.0 * oo2e * (v8_0_0 - rho_e * v8_0_1);
-            const VT v9_4_0 = QCx * v9_1_0 + WQx * v9_1_1 + (VT)1.0 * oo2e * (v9_0_0 - rho_e * v9_0_1);
-            const VT v1_5_0 = QCx * v1_2_0 + WQx * v1_2_1 + (VT)1.0 * oo2ze * v0_2_1;
-            const VT v2_5_0 = QCx * v2_2_0 + WQx * v2_2_1;
-            const VT v3_5_0 = QCx * v3_2_0 + WQx * v3_2_1;
-            const VT v4_5_0 = QCx * v4_2_0 + WQx * v4_2_1 + (VT)2.0 * oo2ze * v1_2_1;
-            const VT v5_5_0 = QCx * v5_2_0 + WQx * v5_2_1 + (VT)1.0 * oo2ze * v2_2_1;
-            const VT v6_5_0 = QCx * v6_2_0 + WQx * v6_2_1 + (VT)1.0 * oo2ze * v3_2_1;
-            const VT v7_5_0 = QCx * v7_2_0 + WQx * v7_2_1;
-            const VT v8_5_0 = QCx * v8_2_0 + WQx * v8_2_1;
-            const VT v9_5_0 = QCx * v9_2_0 + WQx * v9_2_1;
-            const VT v1_6_0 = QCx * v1_3_0 + WQx * v1_3_1 + (VT)1.0 * oo2ze * v0_3_1;
-            const VT v2_6_0 = QCx * v2_3_0 + WQx * v2_3_1;
-            const VT v3_6_0 = QCx * v3_3_0 + WQx * v3_3_1;
-            const VT v4_6_0 = QCx * v4_3_0 + WQx * v4_3_1 + (VT)2.0 * oo2ze * v1_3_1;
-            const VT v5_6_0 = QCx * v5_3_0 + WQx * v5_3_1 + (VT)1.0 * oo2ze * v2_3_1;
-            const VT v6_6_0 = QCx * v6_3_0 + WQx * v6_3_1 + (VT)1.0 * oo2ze * v3_3_1;
-            const VT v7_6_0 = QCx * v7_3_0 + WQx * v7_3_1;
-            const VT v8_6_0 = QCx * v8_3_0 + WQx * v8_3_1;
-            const VT v9_6_0 = QCx * v9_3_0 + WQx * v9_3_1;
-            const VT v1_7_0 = QCy * v1_2_0 + WQy * v1_2_1 + (VT)1.0 * oo2e * (v1_0_0 - rho_e * v1_0_1);
-            const VT v2_7_0 = QCy * v2_2_0 + WQy * v2_2_1 + (VT)1.0 * oo2ze * v0_2_1 + (VT)1.0 * oo2e * (v2_0_0 - rho_e * v2_0_1);
-            const VT v3_7_0 = QCy * v3_2_0 + WQy * v3_2_1 + (VT)1.0 * oo2e * (v3_0_0 - rho_e * v3_0_1);
-            const VT v4_7_0 = QCy * v4_2_0 + WQy * v4_2_1 + (VT)1.0 * oo2e * (v4_0_0 - rho_e * v4_0_1);
-            const VT v5_7_0 = QCy * v5_2_0 + WQy * v5_2_1 + (VT)1.0 * oo2ze * v1_2_1 + (VT)1.0 * oo2e * (v5_0_0 - rho_e * v5_0_1);
-            const VT v6_7_0 = QCy * v6_2_0 + WQy * v6_2_1 + (VT)1.0 * oo2e * (v6_0_0 - rho_e * v6_0_1);
-            const VT v7_7_0 = QCy * v7_2_0 + WQy * v7_2_1 + (VT)2.0 * oo2ze * v2_2_1 + (VT)1.0 * oo2e * (v7_0_0 - rho_e * v7_0_1);
-            const VT v8_7_0 = QCy * v8_2_0 + WQy * v8_2_1 + (VT)1.0 * oo2ze * v3_2_1 + (VT)1.0 * oo2e * (v8_0_0 - rho_e * v8_0_1);
-            const VT v9_7_0 = QCy * v9_2_0 + WQy * v9_2_1 + (VT)1.0 * oo2e * (v9_0_0 - rho_e * v9_0_1);
-            const VT v1_8_0 = QCy * v1_3_0 + WQy * v1_3_1;
-            const VT v2_8_0 = QCy * v2_3_0 + WQy * v2_3_1 + (VT)1.0 * oo2ze * v0_3_1;
-            const VT v3_8_0 = QCy * v3_3_0 + WQy * v3_3_1;
-            const VT v4_8_0 = QCy * v4_3_0 + WQy * v4_3_1;
-            const VT v5_8_0 = QCy * v5_3_0 + WQy * v5_3_1 + (VT)1.0 * oo2ze * v1_3_1;
-            const VT v6_8_0 = QCy * v6_3_0 + WQy * v6_3_1;
-            const VT v7_8_0 = QCy * v7_3_0 + WQy * v7_3_1 + (VT)2.0 * oo2ze * v2_3_1;
-            const VT v8_8_0 = QCy * v8_3_0 + WQy * v8_3_1 + (VT)1.0 * oo2ze * v3_3_1;
-            const VT v9_8_0 = QCy * v9_3_0 + WQy * v9_3_1;
-            const VT v1_9_0 = QCz * v1_3_0 + WQz * v1_3_1 + (VT)1.0 * oo2e * (v1_0_0 - rho_e * v1_0_1);
-            const VT v2_9_0 = QCz * v2_3_0 + WQz * v2_3_1 + (VT)1.0 * oo2e * (v2_0_0 - rho_e * v2_0_1);
-            const VT v3_9_0 = QCz * v3_3_0 + WQz * v3_3_1 + (VT)1.0 * oo2ze * v0_3_1 + (VT)1.0 * oo2e * (v3_0_0 - rho_e * v3_0_1);
-            const VT v4_9_0 = QCz * v4_3_0 + WQz * v4_3_1 + (VT)1.0 * oo2e * (v4_0_0 - rho_e * v4_0_1);
-            const VT v5_9_0 = QCz * v5_3_0 + WQz * v5_3_1 + (VT)1.0 * oo2e * (v5_0_0 - rho_e * v5_0_1);
-            const VT v6_9_0 = QCz * v6_3_0 + WQz * v6_3_1 + (VT)1.0 * oo2ze * v1_3_1 + (VT)1.0 * oo2e * (v6_0_0 - rho_e * v6_0_1);
-            const VT v7_9_0 = QCz * v7_3_0 + WQz * v7_3_1 + (VT)1.0 * oo2e * (v7_0_0 - rho_e * v7_0_1);
-            const VT v8_9_0 = QCz * v8_3_0 + WQz * v8_3_1 + (VT)1.0 * oo2ze * v2_3_1 + (VT)1.0 * oo2e * (v8_0_0 - rho_e * v8_0_1);
-            const VT v9_9_0 = QCz * v9_3_0 + WQz * v9_3_1 + (VT)2.0 * oo2ze * v3_3_1 + (VT)1.0 * oo2e * (v9_0_0 - rho_e * v9_0_1);
-            acc[0] += (double)v1_1_0;
-            acc[1] += (double)v1_2_0;
-            acc[2] += (double)v1_3_0;
-            acc[3] += (double)v1_4_0;
-            acc[4] += (double)v1_5_0;
-            acc[5] += (double)v1_6_0;
-            acc[6] += (double)v1_7_0;
-            acc[7] += (double)v1_8_0;
-            acc[8] += (double)v1_9_0;
-            acc[9] += (double)v2_1_0;
-            acc[10] += (double)v2_2_0;
-            acc[11] += (double)v2_3_0;
-            acc[12] += (double)v2_4_0;
-            acc[13] += (double)v2_5_0;
-            acc[14] += (double)v2_6_0;
-            acc[15] += (double)v2_7_0;
-            acc[16] += (double)v2_8_0;
-            acc[17] += (double)v2_9_0;
-            acc[18] += (double)v3_1_0;
-            acc[19] += (double)v3_2_0;
-            acc[20] += (double)v3_3_0;
-            acc[21] += (double)v3_4_0;
-            acc[22] += (double)v3_5_0;
-            acc[23] += (double)v3_6_0;
-            acc[24] += (double)v3_7_0;
-            acc[25] += (double)v3_8_0;
-            acc[26] += (double)v3_9_0;
-            acc[27] += (double)v4_1_0;
-            acc[28] += (double)v4_2_0;
-            acc[29] += (double)v4_3_0;
-            acc[30] += (double)v4_4_0;
-            acc[31] += (double)v4_5_0;
-            acc[32] += (double)v4_6_0;
-            acc[33] += (double)v4_7_0;
-            acc[34] += (double)v4_8_0;
-            acc[35] += (double)v4_9_0;
-            acc[36] += (double)v5_1_0;
-            acc[37] += (double)v5_2_0;
-            acc[38] += (double)v5_3_0;
-            acc[39] += (double)v5_4_0;
-            acc[40] += (double)v5_5_0;
-            acc[41] += (double)v5_6_0;
-            acc[42] += (double)v5_7_0;
-            acc[43] += (double)v5_8_0;
-            acc[44] += (double)v5_9_0;
-            acc[45] += (double)v6_1_0;
-            acc[46] += (double)v6_2_0;
-            acc[47] += (double)v6_3_0;
-            acc[48] += (double)v6_4_0;
-            acc[49] += (double)v6_5_0;
-            acc[50] += (double)v6_6_0;
-            acc[51] += (double)v6_7_0;
-            acc[52] += (double)v6_8_0;
-            acc[53] += (double)v6_9_0;
-            acc[54] += (double)v7_1_0;
-            acc[55] += (double)v7_2_0;
-            acc[56] += (double)v7_3_0;
-            acc[57] += (double)v7_4_0;
-            acc[58] += (double)v7_5_0;
-            acc[59] += (double)v7_6_0;
-            acc[60] += (double)v7_7_0;
-            acc[61] += (double)v7_8_0;
-            acc[62] += (double)v7_9_0;
-            acc[63] += (double)v8_1_0;
-            acc[64] += (double)v8_2_0;
-            acc[65] += (double)v8_3_0;
-            acc[66] += (double)v8_4_0;
-            acc[67] += (double)v8_5_0;
-            acc[68] += (double)v8_6_0;
-            acc[69] += (double)v8_7_0;
-            acc[70] += (double)v8_8_0;
-            acc[71] += (double)v8_9_0;
-            acc[72] += (double)v9_1_0;
-            acc[73] += (double)v9_2_0;
-            acc[74] += (double)v9_3_0;
-            acc[75] += (double)v9_4_0;
-            acc[76] += (double)v9_5_0;
-            acc[77] += (double)v9_6_0;
-            acc[78] += (double)v9_7_0;
-            acc[79] += (double)v9_8_0;
-            acc[80] += (double)v9_9_0;
+            if constexpr (sizeof(VT) == 8) {
+                acc[0] += (double)v1_1_0;
+                acc[1] += (double)v1_2_0;
+                acc[2] += (double)v1_3_0;
+                acc[3] = fma(QCx, v1_1_0, fma(WQx, v1_1_1, fma(1.0 * oo2ze, v0_1_1, fma(1.0 * oo2e, (v1_0_0 - rho_e * v1_0_1), acc[3]))));
+                acc[4] = fma(QCx, v1_2_0, fma(WQx, v1_2_1, fma(1.0 * oo2ze, v0_2_1, acc[4])));
+                acc[5] = fma(QCx, v1_3_0, fma(WQx, v1_3_1, fma(1.0 * oo2ze, v0_3_1, acc[5])));
+                acc[6] = fma(QCy, v1_2_0, fma(WQy, v1_2_1, fma(1.0 * oo2e, (v1_0_0 - rho_e * v1_0_1), acc[6])));
+                acc[7] = fma(QCy, v1_3_0, fma(WQy, v1_3_1, acc[7]));
+                acc[8] = fma(QCz, v1_3_0, fma(WQz, v1_3_1, fma(1.0 * oo2e, (v1_0_0 - rho_e * v1_0_1), acc[8])));
+                acc[9] += (double)v2_1_0;
+                acc[10] += (double)v2_2_0;
+                acc[11] += (double)v2_3_0;
+                acc[12] = fma(QCx, v2_1_0, fma(WQx, v2_1_1, fma(1.0 * oo2e, (v2_0_0 - rho_e * v2_0_1), acc[12])));
+                acc[13] = fma(QCx, v2_2_0, fma(WQx, v2_2_1, acc[13]));
+                acc[14] = fma(QCx, v2_3_0, fma(WQx, v2_3_1, acc[14]));
+                acc[15] = fma(QCy, v2_2_0, fma(WQy, v2_2_1, fma(1.0 * oo2ze, v0_2_1, fma(1.0 * oo2e, (v2_0_0 - rho_e * v2_0_1), acc[15]))));
+                acc[16] = fma(QCy, v2_3_0, fma(WQy, v2_3_1, fma(1.0 * oo2ze, v0_3_1, acc[16])));
+                acc[17] = fma(QCz, v2_3_0, fma(WQz, v2_3_1, fma(1.0 * oo2e, (v2_0_0 - rho_e * v2_0_1), acc[17])));
+                acc[18] += (double)v3_1_0;
+                acc[19] += (double)v3_2_0;
+                acc[20] += (double)v3_3_0;
+                acc[21] = fma(QCx, v3_1_0, fma(WQx, v3_1_1, fma(1.0 * oo2e, (v3_0_0 - rho_e * v3_0_1), acc[21])));
+                acc[22] = fma(QCx, v3_2_0, fma(WQx, v3_2_1, acc[22]));
+                acc[23] = fma(QCx, v3_3_0, fma(WQx, v3_3_1, acc[23]));
+                acc[24] = fma(QCy, v3_2_0, fma(WQy, v3_2_1, fma(1.0 * oo2e, (v3_0_0 - rho_e * v3_0_1), acc[24])));
+                acc[25] = fma(QCy, v3_3_0, fma(WQy, v3_3_1, acc[25]));
+                acc[26] = fma(QCz, v3_3_0, fma(WQz, v3_3_1, fma(1.0 * oo2ze, v0_3_1, fma(1.0 * oo2e, (v3_0_0 - rho_e * v3_0_1), acc[26]))));
+                acc[27] += (double)v4_1_0;
+                acc[28] += (double)v4_2_0;
+                acc[29] += (double)v4_3_0;
+                acc[30] = fma(QCx, v4_1_0, fma(WQx, v4_1_1, fma(2.0 * oo2ze, v1_1_1, fma(1.0 * oo2e, (v4_0_0 - rho_e * v4_0_1), acc[30]))));
+                acc[31] = fma(QCx, v4_2_0, fma(WQx, v4_2_1, fma(2.0 * oo2ze, v1_2_1, acc[31])));
+                acc[32] = fma(QCx, v4_3_0, fma(WQx, v4_3_1, fma(2.0 * oo2ze, v1_3_1, acc[32])));
+                acc[33] = fma(QCy, v4_2_0, fma(WQy, v4_2_1, fma(1.0 * oo2e, (v4_0_0 - rho_e * v4_0_1), acc[33])));
+                acc[34] = fma(QCy, v4_3_0, fma(WQy, v4_3_1, acc[34]));
+                acc[35] = fma(QCz, v4_3_0, fma(WQz, v4_3_1, fma(1.0 * oo2e, (v4_0_0 - rho_e * v4_0_1), acc[35])));
+                acc[36] += (double)v5_1_0;
+                acc[37] += (double)v5_2_0;
+                acc[38] += (double)v5_3_0;
+                acc[39] = fma(QCx, v5_1_0, fma(WQx, v5_1_1, fma(1.0 * oo2ze, v2_1_1, fma(1.0 * oo2e, (v5_0_0 - rho_e * v5_0_1), acc[39]))));
+                acc[40] = fma(QCx, v5_2_0, fma(WQx, v5_2_1, fma(1.0 * oo2ze, v2_2_1, acc[40])));
+                acc[41] = fma(QCx, v5_3_0, fma(WQx, v5_3_1, fma(1.0 * oo2ze, v2_3_1, acc[41])));
+                acc[42] = fma(QCy, v5_2_0, fma(WQy, v5_2_1, fma(1.0 * oo2ze, v1_2_1, fma(1.0 * oo2e, (v5_0_0 - rho_e * v5_0_1), acc[42]))));
+                acc[43] = fma(QCy, v5_3_0, fma(WQy, v5_3_1, fma(1.0 * oo2ze, v1_3_1, acc[43])));
+                acc[44] = fma(QCz, v5_3_0, fma(WQz, v5_3_1, fma(1.0 * oo2e, (v5_0_0 - rho_e * v5_0_1), acc[44])));
+                acc[45] += (double)v6_1_0;
+                acc[46] += (double)v6_2_0;
+                acc[47] += (double)v6_3_0;
+                acc[48] = fma(QCx, v6_1_0, fma(WQx, v6_1_1, fma(1.0 * oo2ze, v3_1_1, fma(1.0 * oo2e, (v6_0_0 - rho_e * v6_0_1), acc[48]))));
+                acc[49] = fma(QCx, v6_2_0, fma(WQx, v6_2_1, fma(1.0 * oo2ze, v3_2_1, acc[49])));
+                acc[50] = fma(QCx, v6_3_0, fma(WQx, v6_3_1, fma(1.0 * oo2ze, v3_3_1, acc[50])));
+                acc[51] = fma(QCy, v6_2_0, fma(WQy, v6_2_1, fma(1.0 * oo2e, (v6_0_0 - rho_e * v6_0_1), acc[51])));
+                acc[52] = fma(QCy, v6_3_0, fma(WQy, v6_3_1, acc[52]));
+                acc[53] = fma(QCz, v6_3_0, fma(WQz, v6_3_1, fma(1.0 * oo2ze, v1_3_1, fma(1.0 * oo2e, (v6_0_0 - rho_e * v6_0_1), acc[53]))));
+                acc[54] += (double)v7_1_0;
+                acc[55] += (double)v7_2_0;
+                acc[56] += (double)v7_3_0;
+                acc[57] = fma(QCx, v7_1_0, fma(WQx, v7_1_1, fma(1.0 * oo2e, (v7_0_0 - rho_e * v7_0_1), acc[57])));
+                acc[58] = fma(QCx, v7_2_0, fma(WQx, v7_2_1, acc[58]));
+                acc[59] = fma(QCx, v7_3_0, fma(WQx, v7_3_1, acc[59]));
+                acc[60] = fma(QCy, v7_2_0, fma(WQy, v7_2_1, fma(2.0 * oo2ze, v2_2_1, fma(1.0 * oo2e, (v7_0_0 - rho_e * v7_0_1), acc[60]))));
+                acc[61] = fma(QCy, v7_3_0, fma(WQy, v7_3_1, fma(2.0 * oo2ze, v2_3_1, acc[61])));
+                acc[62] = fma(QCz, v7_3_0, fma(WQz, v7_3_1, fma(1.0 * oo2e, (v7_0_0 - rho_e * v7_0_1), acc[62])));
+                acc[63] += (double)v8_1_0;
+                acc[64] += (double)v8_2_0;
+                acc[65] += (double)v8_3_0;
+                acc[66] = fma(QCx, v8_1_0, fma(WQx, v8_1_1, fma(1.0 * oo2e, (v8_0_0 - rho_e * v8_0_1), acc[66])));
+                acc[67] = fma(QCx, v8_2_0, fma(WQx, v8_2_1, acc[67]));
+                acc[68] = fma(QCx, v8_3_0, fma(WQx, v8_3_1, acc[68]));
+                acc[69] = fma(QCy, v8_2_0, fma(WQy, v8_2_1, fma(1.0 * oo2ze, v3_2_1, fma(1.0 * oo2e, (v8_0_0 - rho_e * v8_0_1), acc[69]))));
+                acc[70] = fma(QCy, v8_3_0, fma(WQy, v8_3_1, fma(1.0 * oo2ze, v3_3_1, acc[70])));
+                acc[71] = fma(QCz, v8_3_0, fma(WQz, v8_3_1, fma(1.0 * oo2ze, v2_3_1, fma(1.0 * oo2e, (v8_0_0 - rho_e * v8_0_1), acc[71]))));
+                acc[72] += (double)v9_1_0;
+                acc[73] += (double)v9_2_0;
+                acc[74] += (double)v9_3_0;
+                acc[75] = fma(QCx, v9_1_0, fma(WQx, v9_1_1, fma(1.0 * oo2e, (v9_0_0 - rho_e * v9_0_1), acc[75])));
+                acc[76] = fma(QCx, v9_2_0, fma(WQx, v9_2_1, acc[76]));
+                acc[77] = fma(QCx, v9_3_0, fma(WQx, v9_3_1, acc[77]));
+                acc[78] = fma(QCy, v9_2_0, fma(WQy, v9_2_1, fma(1.0 * oo2e, (v9_0_0 - rho_e * v9_0_1), acc[78])));
+                acc[79] = fma(QCy, v9_3_0, fma(WQy, v9_3_1, acc[79]));
+                acc[80] = fma(QCz, v9_3_0, fma(WQz, v9_3_1, fma(2.0 * oo2ze, v3_3_1, fma(1.0 * oo2e, (v9_0_0 - rho_e * v9_0_1), acc[80]))));
+            } else {
+                acc[0] += (double)v1_1_0;
+                acc[1] += (double)v1_2_0;
+                acc[2] += (double)v1_3_0;
+                const VT v1_4_0 = QCx * v1_1_0 + WQx * v1_1_1 + (VT)1.0 * oo2ze * v0_1_1 + (VT)1.0 * oo2e * (v1_0_0 - rho_e * v1_0_1);
+                acc[3] += (double)v1_4_0;
+                const VT v1_5_0 = QCx * v1_2_0 + WQx * v1_2_1 + (VT)1.0 * oo2ze * v0_2_1;
+                acc[4] += (double)v1_5_0;
+                const VT v1_6_0 = QCx * v1_3_0 + WQx * v1_3_1 + (VT)1.0 * oo2ze * v0_3_1;
+                acc[5] += (double)v1_6_0;
+                const VT v1_7_0 = QCy * v1_2_0 + WQy * v1_2_1 + (VT)1.0 * oo2e * (v1_0_0 - rho_e * v1_0_1);
+                acc[6] += (double)v1_7_0;
+                const VT v1_8_0 = QCy * v1_3_0 + WQy * v1_3_1;
+                acc[7] += (double)v1_8_0;
+                const VT v1_9_0 = QCz * v1_3_0 + WQz * v1_3_1 + (VT)1.0 * oo2e * (v1_0_0 - rho_e * v1_0_1);
+                acc[8] += (double)v1_9_0;
+                acc[9] += (double)v2_1_0;
+                acc[10] += (double)v2_2_0;
+                acc[11] += (double)v2_3_0;
+                const VT v2_4_0 = QCx * v2_1_0 + WQx * v2_1_1 + (VT)1.0 * oo2e * (v2_0_0 - rho_e * v2_0_1);
+                acc[12] += (double)v2_4_0;
+                const VT v2_5_0 = QCx * v2_2_0 + WQx * v2_2_1;
+                acc[13] += (double)v2_5_0;
+                const VT v2_6_0 = QCx * v2_3_0 + WQx * v2_3_1;
+                acc[14] += (double)v2_6_0;
+                const VT v2_7_0 = QCy * v2_2_0 + WQy * v2_2_1 + (VT)1.0 * oo2ze * v0_2_1 + (VT)1.0 * oo2e * (v2_0_0 - rho_e * v2_0_1);
+                acc[15] += (double)v2_7_0;
+                const VT v2_8_0 = QCy * v2_3_0 + WQy * v2_3_1 + (VT)1.0 * oo2ze * v0_3_1;
+                acc[16] += (double)v2_8_0;
+                const VT v2_9_0 = QCz * v2_3_0 + WQz * v2_3_1 + (VT)1.0 * oo2e * (v2_0_0 - rho_e * v2_0_1);
+                acc[17] += (double)v2_9_0;
+                acc[18] += (double)v3_1_0;
+                acc[19] += (double)v3_2_0;
+                acc[20] += (double)v3_3_0;
+                const VT v3_4_0 = QCx * v3_1_0 + WQx * v3_1_1 + (VT)1.0 * oo2e * (v3_0_0 - rho_e * v3_0_1);
+                acc[21] += (double)v3_4_0;
+                const VT v3_5_0 = QCx * v3_2_0 + WQx * v3_2_1;
+                acc[22] += (double)v3_5_0;
+                const VT v3_6_0 = QCx * v3_3_0 + WQx * v3_3_1;
+                acc[23] += (double)v3_6_0;
+                const VT v3_7_0 = QCy * v3_2_0 + WQy * v3_2_1 + (VT)1.0 * oo2e * (v3_0_0 - rho_e * v3_0_1);
+                acc[24] += (double)v3_7_0;
+                const VT v3_8_0 = QCy * v3_3_0 + WQy * v3_3_1;
+                acc[25] += (double)v3_8_0;
+                const VT v3_9_0 = QCz * v3_3_0 + WQz * v3_3_1 + (VT)1.0 * oo2ze * v0_3_1 + (VT)1.0 * oo2e * (v3_0_0 - rho_e * v3_0_1);
+                acc[26] += (double)v3_9_0;
+                acc[27] += (double)v4_1_0;
+                acc[28] += (double)v4_2_0;
+                acc[29] += (double)v4_3_0;
+                const VT v4_4_0 = QCx * v4_1_0 + WQx * v4_1_1 + (VT)2.0 * oo2ze * v1_1_1 + (VT)1.0 * oo2e * (v4_0_0 - rho_e * v4_0_1);
+                acc[30] += (double)v4_4_0;
+                const VT v4_5_0 = QCx * v4_2_0 + WQx * v4_2_1 + (VT)2.0 * oo2ze * v1_2_1;
+                acc[31] += (double)v4_5_0;
+                const VT v4_6_0 = QCx * v4_3_0 + WQx * v4_3_1 + (VT)2.0 * oo2ze * v1_3_1;
+                acc[32] += (double)v4_6_0;
+                const VT v4_7_0 = QCy * v4_2_0 + WQy * v4_2_1 + (VT)1.0 * oo2e * (v4_0_0 - rho_e * v4_0_1);
+                acc[33] += (double)v4_7_0;
+                const VT v4_8_0 = QCy * v4_3_0 + WQy * v4_3_1;
+                acc[34] += (double)v4_8_0;
+                const VT v4_9_0 = QCz * v4_3_0 + WQz * v4_3_1 + (VT)1.0 * oo2e * (v4_0_0 - rho_e * v4_0_1);
+                acc[35] += (double)v4_9_0;
+                acc[36] += (double)v5_1_0;
+                acc[37] += (double)v5_2_0;
+                acc[38] += (double)v5_3_0;
+                const VT v5_4_0 = QCx * v5_1_0 + WQx * v5_1_1 + (VT)1.0 * oo2ze * v2_1_1 + (VT)1.0 * oo2e * (v5_0_0 - rho_e * v5_0_1);
+                acc[39] += (double)v5_4_0;
+                const VT v5_5_0 = QCx * v5_2_0 + WQx * v5_2_1 + (VT)1.0 * oo2ze * v2_2_1;
+                acc[40] += (double)v5_5_0;
+                const VT v5_6_0 = QCx * v5_3_0 + WQx * v5_3_1 + (VT)1.0 * oo2ze * v2_3_1;
+                acc[41] += (double)v5_6_0;
+                const VT v5_7_0 = QCy * v5_2_0 + WQy * v5_2_1 + (VT)1.0 * oo2ze * v1_2_1 + (VT)1.0 * oo2e * (v5_0_0 - rho_e * v5_0_1);
+                acc[42] += (double)v5_7_0;
+                const VT v5_8_0 = QCy * v5_3_0 + WQy * v5_3_1 + (VT)1.0 * oo2ze * v1_3_1;
+                acc[43] += (double)v5_8_0;
+                const VT v5_9_0 = QCz * v5_3_0 + WQz * v5_3_1 + (VT)1.0 * oo2e * (v5_0_0 - rho_e * v5_0_1);
+                acc[44] += (double)v5_9_0;
+                acc[45] += (double)v6_1_0;
+                acc[46] += (double)v6_2_0;
+                acc[47] += (double)v6_3_0;
+                const VT v6_4_0 = QCx * v6_1_0 + WQx * v6_1_1 + (VT)1.0 * oo2ze * v3_1_1 + (VT)1.0 * oo2e * (v6_0_0 - rho_e * v6_0_1);
+                acc[48] += (double)v6_4_0;
+                const VT v6_5_0 = QCx * v6_2_0 + WQx * v6_2_1 + (VT)1.0 * oo2ze * v3_2_1;
+                acc[49] += (double)v6_5_0;
+                const VT v6_6_0 = QCx * v6_3_0 + WQx * v6_3_1 + (VT)1.0 * oo2ze * v3_3_1;
+                acc[50] += (double)v6_6_0;
+                const VT v6_7_0 = QCy * v6_2_0 + WQy * v6_2_1 + (VT)1.0 * oo2e * (v6_0_0 - rho_e * v6_0_1);
+                acc[51] += (double)v6_7_0;
+                const VT v6_8_0 = QCy * v6_3_0 + WQy * v6_3_1;
+                acc[52] += (double)v6_8_0;
+                const VT v6_9_0 = QCz * v6_3_0 + WQz * v6_3_1 + (VT)1.0 * oo2ze * v1_3_1 + (VT)1.0 * oo2e * (v6_0_0 - rho_e * v6_0_1);
+                acc[53] += (double)v6_9_0;
+                acc[54] += (double)v7_1_0;
+                acc[55] += (double)v7_2_0;
+                acc[56] += (double)v7_3_0;
+                const VT v7_4_0 = QCx * v7_1_0 + WQx * v7_1_1 + (VT)1.0 * oo2e * (v7_0_0 - rho_e * v7_0_1);
+                acc[57] += (double)v7_4_0;
+                const VT v7_5_0 = QCx * v7_2_0 + WQx * v7_2_1;
+                acc[58] += (double)v7_5_0;
+                const VT v7_6_0 = QCx * v7_3_0 + WQx * v7_3_1;
+                acc[59] += (double)v7_6_0;
+                const VT v7_7_0 = QCy * v7_2_0 + WQy * v7_2_1 + (VT)2.0 * oo2ze * v2_2_1 + (VT)1.0 * oo2e * (v7_0_0 - rho_e * v7_0_1);
+                acc[60] += (double)v7_7_0;
+                const VT v7_8_0 = QCy * v7_3_0 + WQy * v7_3_1 + (VT)2.0 * oo2ze * v2_3_1;
+                acc[61] += (double)v7_8_0;
+                const VT v7_9_0 = QCz * v7_3_0 + WQz * v7_3_1 + (VT)1.0 * oo2e * (v7_0_0 - rho_e * v7_0_1);
+                acc[62] += (double)v7_9_0;
+                acc[63] += (double)v8_1_0;
+                acc[64] += (double)v8_2_0;
+                acc[65] += (double)v8_3_0;
+                const VT v8_4_0 = QCx * v8_1_0 + WQx * v8_1_1 + (VT)1.0 * oo2e * (v8_0_0 - rho_e * v8_0_1);
+                acc[66] += (double)v8_4_0;
+                const VT v8_5_0 = QCx * v8_2_0 + WQx * v8_2_1;
+                acc[67] += (double)v8_5_0;
+                const VT v8_6_0 = QCx * v8_3_0 + WQx * v8_3_1;
+                acc[68] += (double)v8_6_0;
+                const VT v8_7_0 = QCy * v8_2_0 + WQy * v8_2_1 + (VT)1.0 * oo2ze * v3_2_1 + (VT)1.0 * oo2e * (v8_0_0 - rho_e * v8_0_1);
+                acc[69] += (double)v8_7_0;
+                const VT v8_8_0 = QCy * v8_3_0 + WQy * v8_3_1 + (VT)1.0 * oo2ze * v3_3_1;
+                acc[70] += (double)v8_8_0;
+                const VT v8_9_0 = QCz * v8_3_0 + WQz * v8_3_1 + (VT)1.0 * oo2ze * v2_3_1 + (VT)1.0 * oo2e * (v8_0_0 - rho_e * v8_0_1);
+                acc[71] += (double)v8_9_0;
+                acc[72] += (double)v9_1_0;
+                acc[73] += (double)v9_2_0;
+                acc[74] += (double)v9_3_0;
+                const VT v9_4_0 = QCx * v9_1_0 + WQx * v9_1_1 + (VT)1.0 * oo2e * (v9_0_0 - rho_e * v9_0_1);
+                acc[75] += (double)v9_4_0;
+                const VT v9_5_0 = QCx * v9_2_0 + WQx * v9_2_1;
+                acc[76] += (double)v9_5_0;
+                const VT v9_6_0 = QCx * v9_3_0 + WQx * v9_3_1;
+                acc[77] += (double)v9_6_0;
+                const VT v9_7_0 = QCy * v9_2_0 + WQy * v9_2_1 + (VT)1.0 * oo2e * (v9_0_0 - rho_e * v9_0_1);
+                acc[78] += (double)v9_7_0;
+                const VT v9_8_0 = QCy * v9_3_0 + WQy * v9_3_1;
+                acc[79] += (double)v9_8_0;
+                const VT v9_9_0 = QCz * v9_3_0 + WQz * v9_3_1 + (VT)2.0 * oo2ze * v3_3_1 + (VT)1.0 * oo2e * (v9_0_0 - rho_e * v9_0_1);
+                acc[80] += (double)v9_9_0;
+            }
         }
     }
 }

@@ -25,13 +25,13 @@ __device__ __forceinline__ void vrr_ppps(const PairTab &P, const BoysTab &B, int
             const double r = rsqrt(bra.zeta + ket.zeta);
             const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
-            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[4];
             boys_fm<3>(T, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
-            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
             const VT WQx = (VT)(zz * PQx), WQy = (VT)(zz * PQy), WQz = (VT)(zz * PQz);
             const VT oo2z = (VT)bra.oo2z, oo2e = (VT)ket.oo2z, oo2ze = (VT)(0.5 * r2);
@@ -64,60 +64,90 @@ __device__ __forceinline__ void vrr_ppps(const PairTab &P, const BoysTab &B, int
             const VT v8_0_1 = PAy * v3_0_1 + WPy * v3_0_2;
             const VT v9_0_0 = PAz * v3_0_0 + WPz * v3_0_1 + (VT)1.0 * oo2z * (v0_0_0 - rho_z * v0_0_1);
             const VT v9_0_1 = PAz * v3_0_1 + WPz * v3_0_2 + (VT)1.0 * oo2z * (v0_0_1 - rho_z * v0_0_2);
-            const VT v1_1_0 = QCx * v1_0_0 + WQx * v1_0_1 + (VT)1.0 * oo2ze * v0_0_1;
-            const VT v2_1_0 = QCx * v2_0_0 + WQx * v2_0_1;
-            const VT v3_1_0 = QCx * v3_0_0 + WQx * v3_0_1;
-            const VT v4_1_0 = QCx * v4_0_0 + WQx * v4_0_1 + (VT)2.0 * oo2ze * v1_0_1;
-            const VT v5_1_0 = QCx * v5_0_0 + WQx * v5_0_1 + (VT)1.0 * oo2ze * v2_0_1;
-            const VT v6_1_0 = QCx * v6_0_0 + WQx * v6_0_1 + (VT)1.0 * oo2ze * v3_0_1;
-            const VT v7_1_0 = QCx * v7_0_0 + WQx * v7_0_1;
-            const VT v8_1_0 = QCx * v8_0_0 + WQx * v8_0_1;
-            const VT v9_1_0 = QCx * v9_0_0 + WQx * v9_0_1;
-            const VT v1_2_0 = QCy * v1_0_0 + WQy * v1_0_1;
-            const VT v2_2_0 = QCy * v2_0_0 + WQy * v2_0_1 + (VT)1.0 * oo2ze * v0_0_1;
-            const VT v3_2_0 = QCy * v3_0_0 + WQy * v3_0_1;
-            const VT v4_2_0 = QCy * v4_0_0 + WQy * v4_0_1;
-            const VT v5_2_0 = QCy * v5_0_0 + WQy * v5_0_1 + (VT)1.0 * oo2ze * v1_0_1;
-            const VT v6_2_0 = QCy * v6_0_0 + WQy * v6_0_1;
-            const VT v7_2_0 = QCy * v7_0_0 + WQy * v7_0_1 + (VT)2.0 * oo2ze * v2_0_1;
-            const VT v8_2_0 = QCy * v8_0_0 + WQy * v8_0_1 + (VT)1.0 * oo2ze * v3_0_1;
-            const VT v9_2_0 = QCy * v9_0_0 + WQy * v9_0_1;
-            const VT v1_3_0 = QCz * v1_0_0 + WQz * v1_0_1;
-            const VT v2_3_0 = QCz * v2_0_0 + WQz * v2_0_1;
-            const VT v3_3_0 = QCz * v3_0_0 + WQz * v3_0_1 + (VT)1.0 * oo2ze * v0_0_1;
-            const VT v4_3_0 = QCz * v4_0_0 + WQz * v4_0_1;
-            const VT v5_3_0 = QCz * v5_0_0 + WQz * v5_0_1;
-            const VT v6_3_0 = QCz * v6_0_0 + WQz * v6_0_1 + (VT)1.0 * oo2ze * v1_0_1;
-            const VT v7_3_0 = QCz * v7_0_0 + WQz * v7_0_1;
-            const VT v8_3_0 = QCz * v8_0_0 + WQz * v8_0_1 + (VT)1.0 * oo2ze * v2_0_1;
-            const VT v9_3_0 = QCz * v9_0_0 + WQz * v9_0_1 + (VT)2.0 * oo2ze * v3_0_1;
-            acc[0] += (double)v1_1_0;
-            acc[1] += (double)v1_2_0;
-            acc[2] += (double)v1_3_0;
-            acc[3] += (double)v2_1_0;
-            acc[4] += (double)v2_2_0;
-            acc[5] += (double)v2_3_0;
-            acc[6] += (double)v3_1_0;
-            acc[7] += (double)v3_2_0;
-            acc[8] += (double)v3_3_0;
-            acc[9] += (double)v4_1_0;
-            acc[10] += (double)v4_2_0;
-            acc[11] += (double)v4_3_0;
-            acc[12] += (double)v5_1_0;
-            acc[13] += (double)v5_2_0;
-            acc[14] += (double)v5_3_0;
-            acc[15] += (double)v6_1_0;
-            acc[16] += (double)v6_2_0;
-            acc[17] += (double)v6_3_0;
-            acc[18] += (double)v7_1_0;
-            acc[19] += (double)v7_2_0;
-            acc[20] += (double)v7_3_0;
-            acc[21] += (double)v8_1_0;
-            acc[22] += (double)v8_2_0;
-            acc[23] += (double)v8_3_0;
-            acc[24] += (double)v9_1_0;
-            acc[25] += (double)v9_2_0;
-            acc[26] += (double)v9_3_0;
+            if constexpr (sizeof(VT) == 8) {
+                acc[0] = fma(QCx, v1_0_0, fma(WQx, v1_0_1, fma(1.0 * oo2ze, v0_0_1, acc[0])));
+                acc[1] = fma(QCy, v1_0_0, fma(WQy, v1_0_1, acc[1]));
+                acc[2] = fma(QCz, v1_0_0, fma(WQz, v1_0_1, acc[2]));
+                acc[3] = fma(QCx, v2_0_0, fma(WQx, v2_0_1, acc[3]));
+                acc[4] = fma(QCy, v2_0_0, fma(WQy, v2_0_1, fma(1.0 * oo2ze, v0_0_1, acc[4])));
+                acc[5] = fma(QCz, v2_0_0, fma(WQz, v2_0_1, acc[5]));
+                acc[6] = fma(QCx, v3_0_0, fma(WQx, v3_0_1, acc[6]));
+                acc[7] = fma(QCy, v3_0_0, fma(WQy, v3_0_1, acc[7]));
+                acc[8] = fma(QCz, v3_0_0, fma(WQz, v3_0_1, fma(1.0 * oo2ze, v0_0_1, acc[8])));
+                acc[9] = fma(QCx, v4_0_0, fma(WQx, v4_0_1, fma(2.0 * oo2ze, v1_0_1, acc[9])));
+                acc[10] = fma(QCy, v4_0_0, fma(WQy, v4_0_1, acc[10]));
+                acc[11] = fma(QCz, v4_0_0, fma(WQz, v4_0_1, acc[11]));
+                acc[12] = fma(QCx, v5_0_0, fma(WQx, v5_0_1, fma(1.0 * oo2ze, v2_0_1, acc[12])));
+                acc[13] = fma(QCy, v5_0_0, fma(WQy, v5_0_1, fma(1.0 * oo2ze, v1_0_1, acc[13])));
+                acc[14] = fma(QCz, v5_0_0, fma(WQz, v5_0_1, acc[14]));
+                acc[15] = fma(QCx, v6_0_0, fma(WQx, v6_0_1, fma(1.0 * oo2ze, v3_0_1, acc[15])));
+                acc[16] = fma(QCy, v6_0_0, fma(WQy, v6_0_1, acc[16]));
+                acc[17] = fma(QCz, v6_0_0, fma(WQz, v6_0_1, fma(1.0 * oo2ze, v1_0_1, acc[17])));
+                acc[18] = fma(QCx, v7_0_0, fma(WQx, v7_0_1, acc[18]));
+                acc[19] = fma(QCy, v7_0_0, fma(WQy, v7_0_1, fma(2.0 * oo2ze, v2_0_1, acc[19])));
+                acc[20] = fma(QCz, v7_0_0, fma(WQz, v7_0_1, acc[20]));
+                acc[21] = fma(QCx, v8_0_0, fma(WQx, v8_0_1, acc[21]));
+                acc[22] = fma(QCy, v8_0_0, fma(WQy, v8_0_1, fma(1.0 * oo2ze, v3_0_1, acc[22])));
+                acc[23] = fma(QCz, v8_0_0, fma(WQz, v8_0_1, fma(1.0 * oo2ze, v2_0_1, acc[23])));
+                acc[24] = fma(QCx, v9_0_0, fma(WQx, v9_0_1, acc[24]));
+                acc[25] = fma(QCy, v9_0_0, fma(WQy, v9_0_1, acc[25]));
+                acc[26] = fma(QCz, v9_0_0, fma(WQz, v9_0_1, fma(2.0 * oo2ze, v3_0_1, acc[26])));
+            } else {
+                const VT v1_1_0 = QCx * v1_0_0 + WQx * v1_0_1 + (VT)1.0 * oo2ze * v0_0_1;
+                acc[0] += (double)v1_1_0;
+                const VT v1_2_0 = QCy * v1_0_0 + WQy * v1_0_1;
+                acc[1] += (double)v1_2_0;
+                const VT v1_3_0 = QCz * v1_0_0 + WQz * v1_0_1;
+                acc[2] += (double)v1_3_0;
+                const VT v2_1_0 = QCx * v2_0_0 + WQx * v2_0_1;
+                acc[3] += (double)v2_1_0;
+                const VT v2_2_0 = QCy * v2_0_0 + WQy * v2_0_1 + (VT)1.0 * oo2ze * v0_0_1;
+                acc[4] += (double)v2_2_0;
+                const VT v2_3_0 = QCz * v2_0_0 + WQz * v2_0_1;
+                acc[5] += (double)v2_3_0;
+                const VT v3_1_0 = QCx * v3_0_0 + WQx * v3_0_1;
+                acc[6] += (double)v3_1_0;
+                const VT v3_2_0 = QCy * v3_0_0 + WQy * v3_0_1;
+                acc[7] += (double)v3_2_0;
+                const VT v3_3_0 = QCz * v3_0_0 + WQz * v3_0_1 + (VT)1.0 * oo2ze * v0_0_1;
+                acc[8] += (double)v3_3_0;
+                const VT v4_1_0 = QCx * v4_0_0 + WQx * v4_0_1 + (VT)2.0 * oo2ze * v1_0_1;
+                acc[9] += (double)v4_1_0;
+                const VT v4_2_0 = QCy * v4_0_0 + WQy * v4_0_1;
+                acc[10] += (double)v4_2_0;
+                const VT v4_3_0 = QCz * v4_0_0 + WQz * v4_0_1;
+                acc[11] += (double)v4_3_0;
+                const VT v5_1_0 = QCx * v5_0_0 + WQx * v5_0_1 + (VT)1.0 * oo2ze * v2_0_1;
+                acc[12] += (double)v5_1_0;
+                const VT v5_2_0 = QCy * v5_0_0 + WQy * v5_0_1 + (VT)1.0 * oo2ze * v1_0_1;
+                acc[13] += (double)v5_2_0;
+                const VT v5_3_0 = QCz * v5_0_0 + WQz * v5_0_1;
+                acc[14] += (double)v5_3_0;
+                const VT v6_1_0 = QCx * v6_0_0 + WQx * v6_0_1 + (VT)1.0 * oo2ze * v3_0_1;
+                acc[15] += (double)v6_1_0;
+                const VT v6_2_0 = QCy * v6_0_0 + WQy * v6_0_1;
+                acc[16] += (double)v6_2_0;
+                const VT v6_3_0 = QCz * v6_0_0 + WQz * v6_0_1 + (VT)1.0 * oo2ze * v1_0_1;
+                acc[17] += (double)v6_3_0;
+                const VT v7_1_0 = QCx * v7_0_0 + WQx * v7_0_1;
+                acc[18] += (double)v7_1_0;
+                const VT v7_2_0 = QCy * v7_0_0 + WQy * v7_0_1 + (VT)2.0 * oo2ze * v2_0_1;
+                acc[19] += (double)v7_2_0;
+                const VT v7_3_0 = QCz * v7_0_0 + WQz * v7_0_1;
+                acc[20] += (double)v7_3_0;
+                const VT v8_1_0 = QCx * v8_0_0 + WQx * v8_0_1;
+                acc[21] += (double)v8_1_0;
+                const VT v8_2_0 = QCy * v8_0_0 + WQy * v8_0_1 + (VT)1.0 * oo2ze * v3_0_1;
+                acc[22] += (double)v8_2_0;
+                const VT v8_3_0 = QCz * v8_0_0 + WQz * v8_0_1 + (VT)1.0 * oo2ze * v2_0_1;
+                acc[23] += (double)v8_3_0;
+                const VT v9_1_0 = QCx * v9_0_0 + WQx * v9_0_1;
+                acc[24] += (double)v9_1_0;
+                const VT v9_2_0 = QCy * v9_0_0 + WQy * v9_0_1;
+                acc[25] += (double)v9_2_0;
+                const VT v9_3_0 = QCz * v9_0_0 + WQz * v9_0_1 + (VT)2.0 * oo2ze * v3_0_1;
+                acc[26] += (double)v9_3_0;
+            }
         }
     }
 }

@@ -25,13 +25,13 @@ __device__ __forceinline__ void vrr_psps(const PairTab &P, const BoysTab &B, int
             const double r = rsqrt(bra.zeta + ket.zeta);
             const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
-            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[3];
             boys_fm<2>(T, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
-            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
             const VT WQx = (VT)(zz * PQx), WQy = (VT)(zz * PQy), WQz = (VT)(zz * PQz);
             const VT oo2z = (VT)bra.oo2z, oo2e = (VT)ket.oo2z, oo2ze = (VT)(0.5 * r2);
@@ -48,24 +48,15 @@ __device__ __forceinline__ void vrr_psps(const PairTab &P, const BoysTab &B, int
             const VT v2_0_1 = PAy * v0_0_1 + WPy * v0_0_2;
             const VT v3_0_0 = PAz * v0_0_0 + WPz * v0_0_1;
             const VT v3_0_1 = PAz * v0_0_1 + WPz * v0_0_2;
-            const VT v1_1_0 = QCx * v1_0_0 + WQx * v1_0_1 + (VT)1.0 * oo2ze * v0_0_1;
-            const VT v2_1_0 = QCx * v2_0_0 + WQx * v2_0_1;
-            const VT v3_1_0 = QCx * v3_0_0 + WQx * v3_0_1;
-            const VT v1_2_0 = QCy * v1_0_0 + WQy * v1_0_1;
-            const VT v2_2_0 = QCy * v2_0_0 + WQy * v2_0_1 + (VT)1.0 * oo2ze * v0_0_1;
-            const VT v3_2_0 = QCy * v3_0_0 + WQy * v3_0_1;
-            const VT v1_3_0 = QCz * v1_0_0 + WQz * v1_0_1;
-            const VT v2_3_0 = QCz * v2_0_0 + WQz * v2_0_1;
-            const VT v3_3_0 = QCz * v3_0_0 + WQz * v3_0_1 + (VT)1.0 * oo2ze * v0_0_1;
-            acc[0] += (double)v1_1_0;
-            acc[1] += (double)v1_2_0;
-            acc[2] += (double)v1_3_0;
-            acc[3] += (double)v2_1_0;
-            acc[4] += (double)v2_2_0;
-            acc[5] += (double)v2_3_0;
-            acc[6] += (double)v3_1_0;
-            acc[7] += (double)v3_2_0;
-            acc[8] += (double)v3_3_0;
+            acc[0] = fma(QCx, v1_0_0, fma(WQx, v1_0_1, fma(1.0 * oo2ze, v0_0_1, acc[0])));
+            acc[1] = fma(QCy, v1_0_0, fma(WQy, v1_0_1, acc[1]));
+            acc[2] = fma(QCz, v1_0_0, fma(WQz, v1_0_1, acc[2]));
+            acc[3] = fma(QCx, v2_0_0, fma(WQx, v2_0_1, acc[3]));
+            acc[4] = fma(QCy, v2_0_0, fma(WQy, v2_0_1, fma(1.0 * oo2ze, v0_0_1, acc[4])));
+            acc[5] = fma(QCz, v2_0_0, fma(WQz, v2_0_1, acc[5]));
+            acc[6] = fma(QCx, v3_0_0, fma(WQx, v3_0_1, acc[6]));
+            acc[7] = fma(QCy, v3_0_0, fma(WQy, v3_0_1, acc[7]));
+            acc[8] = fma(QCz, v3_0_0, fma(WQz, v3_0_1, fma(1.0 * oo2ze, v0_0_1, acc[8])));
         }
     }
 }

@@ -25,13 +25,13 @@ __device__ __forceinline__ void vrr_psss(const PairTab &P, const BoysTab &B, int
             const double r = rsqrt(bra.zeta + ket.zeta);
             const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
-            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[2];
             boys_fm<1>(T, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
-            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
             const VT WQx = (VT)(zz * PQx), WQy = (VT)(zz * PQy), WQz = (VT)(zz * PQz);
             const VT oo2z = (VT)bra.oo2z, oo2e = (VT)ket.oo2z, oo2ze = (VT)(0.5 * r2);
@@ -41,12 +41,9 @@ __device__ __forceinline__ void vrr_psss(const PairTab &P, const BoysTab &B, int
             (void)oo2z; (void)oo2e; (void)oo2ze; (void)rho_z; (void)rho_e;
             const VT v0_0_0 = (VT)(pref * F[0]);
             const VT v0_0_1 = (VT)(pref * F[1]);
-            const VT v1_0_0 = PAx * v0_0_0 + WPx * v0_0_1;
-            const VT v2_0_0 = PAy * v0_0_0 + WPy * v0_0_1;
-            const VT v3_0_0 = PAz * v0_0_0 + WPz * v0_0_1;
-            acc[0] += (double)v1_0_0;
-            acc[1] += (double)v2_0_0;
-            acc[2] += (double)v3_0_0;
+            acc[0] = fma(PAx, v0_0_0, fma(PQx, (-ez * v0_0_1), acc[0]));
+            acc[1] = fma(PAy, v0_0_0, fma(PQy, (-ez * v0_0_1), acc[1]));
+            acc[2] = fma(PAz, v0_0_0, fma(PQz, (-ez * v0_0_1), acc[2]));
         }
     }
 }

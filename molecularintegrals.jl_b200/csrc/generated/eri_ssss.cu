@@ -25,13 +25,13 @@ __device__ __forceinline__ void vrr_ssss(const PairTab &P, const BoysTab &B, int
             const double r = rsqrt(bra.zeta + ket.zeta);
             const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
-            const double T = bra.zeta * ket.zeta * r2 * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
+            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[1];
             boys_fm<0>(T, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
-            const double ez = ket.zeta * r2, zz = bra.zeta * r2;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
             const VT WQx = (VT)(zz * PQx), WQy = (VT)(zz * PQy), WQz = (VT)(zz * PQz);
             const VT oo2z = (VT)bra.oo2z, oo2e = (VT)ket.oo2z, oo2ze = (VT)(0.5 * r2);
@@ -39,8 +39,8 @@ __device__ __forceinline__ void vrr_ssss(const PairTab &P, const BoysTab &B, int
             (void)PAx; (void)PAy; (void)PAz; (void)QCx; (void)QCy; (void)QCz;
             (void)WPx; (void)WPy; (void)WPz; (void)WQx; (void)WQy; (void)WQz;
             (void)oo2z; (void)oo2e; (void)oo2ze; (void)rho_z; (void)rho_e;
-            const VT v0_0_0 = (VT)(pref * F[0]);
-            acc[0] += (double)v0_0_0;
+
+            acc[0] = fma(pref, F[0], acc[0]);
         }
     }
 }

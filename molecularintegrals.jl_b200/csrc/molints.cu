@@ -42,8 +42,7 @@ struct molints_ctx {
     // stay cached (release threshold = max), so plan creation and destruction neither call
     // cudaMalloc/cudaFree nor synchronise the device.
     cudaMemPool_t pool = nullptr;
-    double *boys_tab = nullptr;
-    double *boys_scaled = nullptr;  // per-M tables F_{M+k}(T_n)/k!, k < 8, and e^-T_n
+    double *boys_tab = nullptr;  // fill_boys_table
     double *out_cache = nullptr;  // device buffer for host-output calls
     int64_t out_cache_len = 0;
     // Two-phase output scratch, shared by the context's plans (it is needed only while an
@@ -784,20 +783,17 @@ void launch_build_pairs(int npair, const int2 *pair_ab, const int4 *info, const 
                                                           nullptr, pp, geo, nullptr, 0);
 }
 
-// The scaled Boys tables of the kernels for M = 0..nM-1: row n of table M holds
-// F_{M+k}(T_n)/k! (k < 8), e^-T_n and a pad, T_n = n/16, n = 0..640.
-void fill_boys_scaled(double *sc, int nM) {
+// The Boys tables of the kernels for M = 0..nM-1, T_n = n/32, n = 0..1280: per M the rows
+// {F_M(T_n), e^-T_n}, then the rows {F_{M+6}(T_n)/6!, F_{M+3}(T_n)/3!}.
+void fill_boys_table(double *tab, int nM) {
     for (int M = 0; M < nM; ++M)
         for (int n = 0; n < kBoysRows; ++n) {
             const double T = n * kBoysStep;
-            double *row = sc + ((size_t)M * kBoysRows + n) * kBoysScaledCols;
-            double fact = 1.0;
-            for (int k = 0; k < kBoysTaylor; ++k) {
-                if (k > 0) fact *= k;
-                row[k] = boys_series(M + k, T) / fact;
-            }
-            row[kBoysTaylor] = std::exp(-T);
-            row[kBoysTaylor + 1] = 0.0;
+            double *row = tab + (size_t)M * (2 * kBoysHalf) + 2 * n;
+            row[0] = boys_series(M, T);
+            row[1] = std::exp(-T);
+            row[kBoysHalf] = boys_series(M + 6, T) / 720.0;
+            row[kBoysHalf + 1] = boys_series(M + 3, T) / 6.0;
         }
 }
 
@@ -936,23 +932,11 @@ int molints_create(molints_ctx **out, int device, int64_t budget, uint32_t flags
     }
     uint64_t keep = UINT64_MAX;
     cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    // Boys table: F_0..F_22 and e^-T at T_n = n/16, n = 0..640.
-    std::vector<double> tab((size_t)kBoysRows * kBoysCols);
-    for (int n = 0; n < kBoysRows; ++n) {
-        const double T = n * kBoysStep;
-        for (int m = 0; m < kBoysCols - 1; ++m) tab[(size_t)n * kBoysCols + m] = boys_series(m, T);
-        tab[(size_t)n * kBoysCols + kBoysCols - 1] = std::exp(-T);
-    }
-    // Per-M tables for the kernels: row n of table M holds F_{M+k}(T_n)/k! (k = 0..7) and
-    // e^-T_n, padded to 10 doubles, so the Taylor sum is a Horner chain of 7 FMAs.
-    std::vector<double> sc((size_t)kBoysMaxM1 * kBoysRows * kBoysScaledCols, 0.0);
-    fill_boys_scaled(sc.data(), kBoysMaxM1);
+    std::vector<double> tab((size_t)kBoysMaxM1 * 2 * kBoysHalf);
+    fill_boys_table(tab.data(), kBoysMaxM1);
     int rc = dev_alloc(ctx, &ctx->boys_tab, tab.size(), nullptr);
-    if (!rc) rc = dev_alloc(ctx, &ctx->boys_scaled, sc.size(), nullptr);
     if (rc) { molints_destroy(ctx); return rc; }
     if (cudaMemcpyAsync(ctx->boys_tab, tab.data(), tab.size() * sizeof(double),
-                        cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess ||
-        cudaMemcpyAsync(ctx->boys_scaled, sc.data(), sc.size() * sizeof(double),
                         cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess ||
         cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
         molints_destroy(ctx);
@@ -977,7 +961,6 @@ int molints_destroy(molints_ctx *ctx) {
     ctx->stream = ctx->own_stream;
     if (ctx->own_stream) {
         dev_free(ctx, ctx->boys_tab);
-        dev_free(ctx, ctx->boys_scaled);
         dev_free(ctx, ctx->out_cache);
         dev_free(ctx, ctx->scratch);
         cudaStreamSynchronize(ctx->own_stream);
@@ -1066,7 +1049,6 @@ int molints_set_stream(molints_ctx *ctx, void *stream) {
 static BoysTab boys_of(const molints_ctx *ctx, int mode) {
     BoysTab bt;
     bt.tab = ctx->boys_tab;
-    bt.scaled = ctx->boys_scaled;
     bt.t_switch = (mode == MOLINTS_BOYS_EXACT) ? kBoysTableMax : kBoysReferenceSwitch;
     return bt;
 }

@@ -35,7 +35,7 @@ namespace molints {
 void launch_build_pairs(int npair, const int2 *pair_ab, const int4 *info, const int *pp_src,
                         const double *xyz, const int *poff, const double *expn,
                         const double *ncoef, PrimPair *pp, double4 *geo, cudaStream_t s);
-void fill_boys_scaled(double *sc, int nM);
+void fill_boys_table(double *tab, int nM);
 }  // namespace molints
 
 using namespace molints;
@@ -45,8 +45,11 @@ namespace {
 constexpr size_t kScratchBytes = (size_t)8 << 20;  // the stated maximum: 8 MiB
 constexpr size_t kAlign = 256;
 constexpr int kTableM = 4 * kLmaxHgp + 1;  // Boys orders the HGP class kernels use
-constexpr size_t kTableBytes =
-    ((size_t)kTableM * kBoysRows * kBoysScaledCols * sizeof(double) + kAlign - 1) / kAlign * kAlign;
+// Bytes kept for the Boys tables (368,928 of them used): the rest of the 8 MiB bounds the bases
+// that are accepted.
+constexpr size_t kTableBytes = 461568;
+static_assert((size_t)kTableM * 2 * kBoysHalf * sizeof(double) <= kTableBytes && kTableBytes % kAlign == 0,
+              "the Boys tables fit their part of the scratch");
 constexpr int kMaxDevices = 64;
 
 // Device scratch.  In host code this name is only a stand-in for the symbol, never an
@@ -165,8 +168,8 @@ extern "C" int molints_eri_packed_noalloc(const molints_basis *b, const molints_
         void *ptr = nullptr;
         e = cudaGetSymbolAddress(&ptr, g_scratch);
         if (e != cudaSuccess || !ptr) return noalloc_fail(err, err_len, MOLINTS_ERR_CUDA, "cudaGetSymbolAddress failed");
-        fill_boys_scaled(reinterpret_cast<double *>(g_host), kTableM);
-        e = cudaMemcpy(ptr, g_host, (size_t)kTableM * kBoysRows * kBoysScaledCols * sizeof(double),
+        fill_boys_table(reinterpret_cast<double *>(g_host), kTableM);
+        e = cudaMemcpy(ptr, g_host, (size_t)kTableM * 2 * kBoysHalf * sizeof(double),
                        cudaMemcpyHostToDevice);
         if (e != cudaSuccess) return noalloc_fail(err, err_len, MOLINTS_ERR_CUDA, "Boys table copy failed");
         g_dev_ptr[dev] = ptr;
@@ -290,8 +293,7 @@ extern "C" int molints_eri_packed_noalloc(const molints_basis *b, const molints_
                        d_pp, d_geo, s);
     PairTab P{d_info, d_geo, d_pp, reinterpret_cast<const double2 *>(data + o_bnd)};
     BoysTab B;
-    B.tab = nullptr;  // the class kernels read only the scaled tables
-    B.scaled = reinterpret_cast<const double *>(base);
+    B.tab = reinterpret_cast<const double *>(base);
     B.t_switch = boys_mode == MOLINTS_BOYS_EXACT ? kBoysTableMax : kBoysReferenceSwitch;
     for (int x = 0; x < kNumPairClasses; ++x)
         for (int y = 0; y <= x; ++y) {
