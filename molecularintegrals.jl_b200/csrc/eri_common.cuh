@@ -125,47 +125,69 @@ __device__ __forceinline__ PrimPair load_pp(const PrimPair *__restrict__ base, i
 //                  farray's Fm_asymp top order and e^-T-free recursion produce.
 // The table index is rounded with the 1.5*2^52 trick: T*32 + 1.5*2^52 holds round(T*32) in
 // its low mantissa bits, and subtracting the constant back gives T_n*32 exactly.
+// The near part: T at most the tables' end.
+template <int M>
+__device__ __forceinline__ void boys_near(double T, const BoysTab &bt, double *F) {
+    static_assert(M < kBoysMaxM1, "Boys order beyond the tables");
+    constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52
+    const double t32 = fma(T, kBoysStepInv, kMagic);
+    // (exponents near the ends of the double range can make T a NaN: the row stays in the table)
+    const unsigned n = min((unsigned)__double2loint(t32), (unsigned)(kBoysRows - 1));
+    const double tn = (t32 - kMagic) * kBoysStep, d = tn - T;
+    const double2 *__restrict__ tab = reinterpret_cast<const double2 *>(bt.tab + (size_t)M * (2 * kBoysHalf)) + n;
+    const double2 fe = __ldg(tab), c63 = __ldg(tab + kBoysRows);
+    // c_k = T_n c_{k+1} 2(k+1)/(2(M+k)+1) + e^-T_n / (k! (2(M+k)+1))
+    const double c5 = fma(tn * c63.x, 12.0 / (2 * M + 11), fe.y * (1.0 / (120.0 * (2 * M + 11))));
+    const double c2 = fma(tn * c63.y, 6.0 / (2 * M + 5), fe.y * (1.0 / (2.0 * (2 * M + 5))));
+    const double c4 = fma(tn * c5, 10.0 / (2 * M + 9), fe.y * (1.0 / (24.0 * (2 * M + 9))));
+    const double c1 = fma(tn * c2, 4.0 / (2 * M + 3), fe.y * (1.0 / (2 * M + 3)));
+    double f = fma(c63.x, d, c5);
+    f = fma(f, d, c4);
+    f = fma(f, d, c63.y);
+    f = fma(f, d, c2);
+    f = fma(f, d, c1);
+    f = fma(f, d, fe.x);
+    F[M] = f;
+    if (M > 0) {
+        // e^d for |d| <= 1/64 by its Taylor polynomial to d^6
+        double ed = fma(d, 1.0 / 720, 1.0 / 120);
+        ed = fma(ed, d, 1.0 / 24);
+        ed = fma(ed, d, 1.0 / 6);
+        ed = fma(ed, d, 0.5);
+        ed = fma(ed, d, 1.0);
+        ed = fma(ed, d, 1.0);
+        const double emt = fe.y * ed;
+        const double t2 = 2.0 * T;
+#pragma unroll
+        for (int m = M - 1; m >= 0; --m) F[m] = fma(t2, F[m + 1], emt) * (1.0 / (2 * m + 1));
+    }
+}
+
 template <int M>
 __device__ __forceinline__ void boys_fm(double T, const BoysTab &bt, double *F) {
-    static_assert(M < kBoysMaxM1, "Boys order beyond the scaled tables");
     if (T < bt.t_switch) {
-        constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52
-        const double t32 = fma(T, kBoysStepInv, kMagic);
-        const int n = __double2loint(t32);
-        const double tn = (t32 - kMagic) * kBoysStep, d = tn - T;
-        const double2 *__restrict__ tab = reinterpret_cast<const double2 *>(bt.tab + (size_t)M * (2 * kBoysHalf)) + n;
-        const double2 fe = __ldg(tab), c63 = __ldg(tab + kBoysRows);
-        // c_k = T_n c_{k+1} 2(k+1)/(2(M+k)+1) + e^-T_n / (k! (2(M+k)+1))
-        const double c5 = fma(tn * c63.x, 12.0 / (2 * M + 11), fe.y * (1.0 / (120.0 * (2 * M + 11))));
-        const double c2 = fma(tn * c63.y, 6.0 / (2 * M + 5), fe.y * (1.0 / (2.0 * (2 * M + 5))));
-        const double c4 = fma(tn * c5, 10.0 / (2 * M + 9), fe.y * (1.0 / (24.0 * (2 * M + 9))));
-        const double c1 = fma(tn * c2, 4.0 / (2 * M + 3), fe.y * (1.0 / (2 * M + 3)));
-        double f = fma(c63.x, d, c5);
-        f = fma(f, d, c4);
-        f = fma(f, d, c63.y);
-        f = fma(f, d, c2);
-        f = fma(f, d, c1);
-        f = fma(f, d, fe.x);
-        F[M] = f;
-        if (M > 0) {
-            // e^d for |d| <= 1/64 by its Taylor polynomial to d^6
-            double ed = fma(d, 1.0 / 720, 1.0 / 120);
-            ed = fma(ed, d, 1.0 / 24);
-            ed = fma(ed, d, 1.0 / 6);
-            ed = fma(ed, d, 0.5);
-            ed = fma(ed, d, 1.0);
-            ed = fma(ed, d, 1.0);
-            const double emt = fe.y * ed;
-            const double t2 = 2.0 * T;
-#pragma unroll
-            for (int m = M - 1; m >= 0; --m) F[m] = fma(t2, F[m + 1], emt) * (1.0 / (2 * m + 1));
-        }
+        boys_near<M>(T, bt, F);
     } else {
         const double r = rsqrt(T);
         F[0] = 0.88622692545275801365 * r;  // sqrt(pi)/2
         const double oo2t = 0.5 * r * r;
 #pragma unroll
         for (int m = 1; m <= M; ++m) F[m] = F[m - 1] * ((2 * m - 1) * oo2t);
+    }
+}
+
+// What the class kernels take: F_0..F_M at T below the switch; far (T at or above it) the asymptotic
+// family times T^(m + 1/2), (2m-1)!! / 2^m * sqrt(pi)/2 (the caller's r and r2 carry the powers of T).
+// (With the asymptotic branch of boys_fm, its own square root included, most warps ran both branches:
+// FARFIG.)
+template <int M>
+__device__ __forceinline__ void boys_scaled(bool far, double T, const BoysTab &bt, double *F) {
+    if (!far) {
+        boys_near<M>(T, bt, F);
+    } else {
+        F[0] = 0.88622692545275801365;  // sqrt(pi)/2
+#pragma unroll
+        for (int m = 1; m <= M; ++m) F[m] = F[m - 1] * (m - 0.5);
     }
 }
 

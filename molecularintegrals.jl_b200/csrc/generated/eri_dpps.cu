@@ -22,14 +22,19 @@ __device__ __forceinline__ void vrr_dpps(const PairTab &P, const BoysTab &B, int
         const PrimPair ket = load_pp(P.pp, ik_.x + j);
         for (int i = i0; i < i1; i += istep) {
             const PrimPair bra = load_pp(P.pp, ib_.x + i);
-            const double r = rsqrt(bra.zeta + ket.zeta);
-            const double r2 = r * r;
             const double PQx = bra.px - ket.px, PQy = bra.py - ket.py, PQz = bra.pz - ket.pz;
+            // near (T below the switch): r = 1/sqrt(zeta+eta), r2 = r^2.  Far: the same recurrences with
+            // r2 = 1/(zeta eta PQ^2) in the place of 1/(zeta+eta) and F_m T^m, constants, in that of
+            // F_m -- each factor of r2 comes with one order of F -- so both take one square root
+            // and a far lane no other work (boys_scaled)
+            const double s = bra.zeta + ket.zeta, ze = bra.zeta * ket.zeta * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const bool far = !(ze < B.t_switch * s);
+            const double r = rsqrt(far ? ze : s);
+            const double r2 = r * r;
             const double ez = ket.zeta * r2, zz = bra.zeta * r2;
-            const double T = bra.zeta * ez * (PQx * PQx + PQy * PQy + PQz * PQz);
             const double pref = bra.kab * ket.kab * r;
             double F[5];
-            boys_fm<4>(T, B, F);
+            boys_scaled<4>(far, ze * r2, B, F);
             const VT PAx = (VT)bra.pax, PAy = (VT)bra.pay, PAz = (VT)bra.paz;
             const VT QCx = (VT)ket.pax, QCy = (VT)ket.pay, QCz = (VT)ket.paz;
             const VT WPx = (VT)(-ez * PQx), WPy = (VT)(-ez * PQy), WPz = (VT)(-ez * PQz);
