@@ -1578,12 +1578,13 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     const size_t t_cm = tv.take<int>(cm_start.size()), t_lane = tv.take<double>(nmol);
     const size_t t_units = tv.take<int4>(tp ? npe_all : 0);
     const size_t up_bytes = tv.at;
-    // cleared before the build: the molecules' Qabs bounds and the summary that is read back
+    // cleared before the build: the molecules' Qabs bounds, the queues' counts and the summary that is read back
     // (class-pair chunk offsets, the count of pairs without kept primitive pairs, class-pair costs,
     // kept primitive pairs, bad-shell flag)
     const size_t t_qmax = tv.take<unsigned long long>(nmol);
     const size_t t_sum = tv.take<long long>(kNumClassPairs + 2), t_ccost = tv.take<double>(kNumClassPairs);
     const size_t t_nkept = tv.take<long long>(1), t_bad = tv.take<int>(1);
+    const size_t t_place = tv.take<unsigned long long>(kNumClassPairs * kCostBuckets);
     const size_t clear_end = tv.at;
     const size_t t_pbound = tv.take<double2>(nall);
     const size_t t_npp1 = tv.take<int>(npair), t_bnd1 = tv.take<double2>(npair);
@@ -1591,9 +1592,8 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     const size_t t_idx1 = tv.take<int>(npair), t_idx2 = tv.take<int>(npair);
     const size_t t_prefix = tv.take<long long>((size_t)npair + 1), t_npp = tv.take<int>((size_t)npair + 1);
     const size_t t_ms = tv.take<int>(npair);
-    const size_t t_cnt = tv.take<long long>((size_t)n_items + 1), t_cost = tv.take<double>(n_items);
-    const size_t t_off = tv.take<long long>((size_t)n_items + 1);
-    const size_t cub_bytes = std::max(plan_build_temp_bytes(npair), queue_count_temp_bytes(n_items));
+    const size_t t_cost = tv.take<double>(n_items);
+    const size_t cub_bytes = plan_build_temp_bytes(npair);
     const size_t t_cub = tv.take<char>(cub_bytes);
     // the plan's buffers, one allocation; what is uploaded comes first, laid out as in the stage
     const int nc2 = kNumPairClasses * kNumPairClasses;
@@ -1805,9 +1805,8 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     QA.region = tp ? p->g_region : nullptr;
     QA.bnd = p->bnd;
     QA.lane_cost = reinterpret_cast<const double *>(tmp + t_lane);
-    QA.cnt = reinterpret_cast<long long *>(tmp + t_cnt);
     QA.cost = reinterpret_cast<double *>(tmp + t_cost);
-    QA.off = reinterpret_cast<long long *>(tmp + t_off);
+    QA.place = reinterpret_cast<unsigned long long *>(tmp + t_place);
     QA.summary = reinterpret_cast<long long *>(tmp + t_sum);
     QA.class_cost = reinterpret_cast<double *>(tmp + t_ccost);
     QA.nkept = reinterpret_cast<long long *>(tmp + t_nkept);
@@ -1842,7 +1841,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
             return cuda_fail(ctx, e, "plan_create bound pass");
         }
         if ((e = cudaGetLastError()) || (e = plan_build_pairs(A, tmp + t_cub, cub_bytes, s)) ||
-            (e = queue_count(S, QA, tmp + t_cub, cub_bytes, s))) {
+            (e = queue_count(S, QA, s))) {
             release_temp(); plan_free(p);
             return cuda_fail(ctx, e, "plan_create device build");
         }
@@ -1876,31 +1875,13 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     p->plan_ms[1] = ms_since(t_phase);
     t_phase = clk::now();
 
-    // ---- the chunks, emitted in (class pair, bra, ket) order and placed by a stable sort on
-    // (class pair, cost bucket): class pairs in order, heaviest bucket first
+    // ---- the chunks, each at its place: class pairs in order, heaviest cost bucket first
     rc = dev_alloc(ctx, &p->chunks, (size_t)std::max<long long>(nq, 1), &p->bytes);
     if (!rc && tp) rc = dev_alloc(ctx, &p->chunk_slot, (size_t)std::max<long long>(nq, 1), &p->bytes);
-    Carve ev;
-    const size_t e_raw = ev.take<int4>(nq), e_key1 = ev.take<unsigned short>(nq), e_key2 = ev.take<unsigned short>(nq);
-    const size_t e_idx1 = ev.take<int>(nq), e_idx2 = ev.take<int>(nq), e_slot = ev.take<long long>(tp ? nq : 0);
-    const size_t emit_cub = queue_emit_temp_bytes(nq);
-    const size_t e_cub = ev.take<char>(emit_cub);
-    char *etmp = nullptr;
-    if (!rc && nq > 0) rc = dev_alloc(ctx, &etmp, ev.at, &temp_tally);
     if (rc) { release_temp(); plan_free(p); return rc; }
     if (nq > 0) {
-        QueueEmitArgs E{};
-        E.raw = reinterpret_cast<int4 *>(etmp + e_raw);
-        E.key1 = reinterpret_cast<unsigned short *>(etmp + e_key1);
-        E.key2 = reinterpret_cast<unsigned short *>(etmp + e_key2);
-        E.idx1 = reinterpret_cast<int *>(etmp + e_idx1);
-        E.idx2 = reinterpret_cast<int *>(etmp + e_idx2);
-        E.raw_slot = tp ? reinterpret_cast<long long *>(etmp + e_slot) : nullptr;
-        E.chunks = p->chunks;
-        E.chunk_slot = tp ? p->chunk_slot : nullptr;
-        E.nq = nq;
-        e = queue_emit(S, QA, E, etmp + e_cub, emit_cub, s);
-        dev_free(ctx, etmp);
+        const QueueEmitArgs E{p->chunks, tp ? p->chunk_slot : nullptr};
+        e = queue_emit(S, QA, E, s);
         if (e != cudaSuccess) { release_temp(); plan_free(p); return cuda_fail(ctx, e, "plan_create work queues"); }
     }
     if (tp && nrows_all > 0) {

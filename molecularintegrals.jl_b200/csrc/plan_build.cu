@@ -172,85 +172,110 @@ __device__ __forceinline__ int item_class_pair(const QueueSetup &S, int t) {
     return lo;
 }
 
+// Calls f(chunk of the stretch, its bucket, leader, lanes of the warp with the same bucket) for the
+// chunks of a stretch, 32 a step; lanes without a chunk pass bucket -1 and f sees only the others.
+template <class F>
+__device__ __forceinline__ void for_chunks(const QueueArgs &A, double wp, int first, int n, int end, int lane, F &&f) {
+    const int nc = (end - first + n - 1) / n;
+    for (int c0 = 0; c0 < nc; c0 += 32) {
+        const int c = c0 + lane, q0 = first + c * n;
+        int b = -1;
+        if (c < nc) b = cost_bucket(wp * (double)(A.npp_prefix[min(q0 + n, end)] - A.npp_prefix[q0]));
+        const unsigned peers = __match_any_sync(0xffffffffu, b);
+        f(q0, b, peers);
+    }
+}
+
+// Pass 1: chunks per (class pair, cost bucket) and cost per item.
 __global__ void queue_count_kernel(const QueueSetup S, QueueArgs A) {
     const int t = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    if (t > A.n_items) return;
-    if (t == A.n_items) {
-        if (lane == 0) A.cnt[t] = 0;
-        return;
-    }
+    if (t >= A.n_items) return;
     const int ci = item_class_pair(S, t);
     const int pb = S.cls_start[S.cx[ci]] + (t - S.item_base[ci]);
-    long long c = 0;
     double total = 0.0;
     const double wp = S.w[ci] * A.npp[pb];
-    walk_item(S, A, ci, pb, lane, [&](int q0, int n, int, int end, int) {
-        c += (end - q0 + n - 1) / n;
-        total += wp * (double)(A.npp_prefix[end] - A.npp_prefix[q0]);
+    walk_item(S, A, ci, pb, lane, [&](int first, int n, int, int end, int) {
+        for_chunks(A, wp, first, n, end, lane, [&](int, int b, unsigned peers) {
+            if (b >= 0 && lane == __ffs(peers) - 1) atomicAdd(&A.place[ci * kCostBuckets + b], (unsigned long long)__popc(peers));
+        });
+        total += wp * (double)(A.npp_prefix[end] - A.npp_prefix[first]);
     });
-    if (lane == 0) {
-        A.cnt[t] = c;
-        A.cost[t] = total;
-    }
+    if (lane == 0) A.cost[t] = total;
 }
 
-// Per class pair: its first chunk (and the queue length last) and its total cost, summed in
-// item order by one block per class pair.
+// Block ci < kNumClassPairs: the class pair's total cost, summed in item order.  The last block: the
+// counts become the first places of each (class pair, cost bucket), class pairs in order and the
+// heaviest bucket first, with every class pair's first chunk and the queue length in the summary.
 __global__ void queue_summary_kernel(const QueueSetup S, QueueArgs A) {
     const int ci = blockIdx.x;
-    if (threadIdx.x == 0) {
-        A.summary[ci] = A.off[S.item_base[ci]];
-        if (ci == kNumClassPairs - 1) {
-            A.summary[kNumClassPairs] = A.off[A.n_items];
-            *A.nkept = A.npp_prefix[A.npair];
+    if (ci < kNumClassPairs) {
+        __shared__ double part[kThreads];
+        double s = 0.0;
+        for (int t = S.item_base[ci] + threadIdx.x; t < S.item_base[ci + 1]; t += blockDim.x) s += A.cost[t];
+        part[threadIdx.x] = s;
+        __syncthreads();
+        for (int h = blockDim.x / 2; h > 0; h >>= 1) {
+            if (threadIdx.x < h) part[threadIdx.x] += part[threadIdx.x + h];
+            __syncthreads();
         }
+        if (threadIdx.x == 0) A.class_cost[ci] = part[0];
+        return;
     }
-    __shared__ double part[kThreads];
-    double s = 0.0;
-    for (int t = S.item_base[ci] + threadIdx.x; t < S.item_base[ci + 1]; t += blockDim.x) s += A.cost[t];
-    part[threadIdx.x] = s;
+    constexpr int kAll = kNumClassPairs * kCostBuckets, kEach = (kAll + kThreads - 1) / kThreads;
+    __shared__ long long before[kThreads + 1];
+    const int e0 = threadIdx.x * kEach, e1 = min(e0 + kEach, kAll);
+    long long sum = 0;
+    for (int e = e0; e < e1; ++e) sum += (long long)A.place[e];
+    before[threadIdx.x + 1] = sum;
+    if (threadIdx.x == 0) before[0] = 0;
     __syncthreads();
-    for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-        if (threadIdx.x < h) part[threadIdx.x] += part[threadIdx.x + h];
+    for (int h = 1; h < kThreads; h <<= 1) {
+        const long long add = threadIdx.x + 1 > h ? before[threadIdx.x + 1 - h] : 0;
+        __syncthreads();
+        before[threadIdx.x + 1] += add;
         __syncthreads();
     }
-    if (threadIdx.x == 0) A.class_cost[ci] = part[0];
+    long long at = before[threadIdx.x];
+    for (int e = e0; e < e1; ++e) {
+        if (e % kCostBuckets == 0) A.summary[e / kCostBuckets] = at;
+        const long long k = (long long)A.place[e];
+        A.place[e] = (unsigned long long)at;
+        at += k;
+    }
+    if (threadIdx.x == kThreads - 1) {
+        A.summary[kNumClassPairs] = before[kThreads];
+        *A.nkept = A.npp_prefix[A.npair];
+    }
 }
 
+// Pass 2: every chunk at the next place of its (class pair, cost bucket).  The order within a bucket
+// is the order of arrival: it decides when a chunk is computed, not what it computes.
 __global__ void queue_emit_kernel(const QueueSetup S, QueueArgs A, QueueEmitArgs E) {
     const int t = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (t >= A.n_items) return;
     const int ci = item_class_pair(S, t);
     const int x = S.cx[ci], y = S.cy[ci];
     const int pb = S.cls_start[x] + (t - S.item_base[ci]);
-    long long d0 = A.off[t];
     const double wp = S.w[ci] * A.npp[pb];
     walk_item(S, A, ci, pb, lane, [&](int first, int n, int lg, int end, int m) {
-        const int nc = (end - first + n - 1) / n;
-        for (int c = lane; c < nc; c += 32) {
-            const int q0 = first + c * n, k = min(n, end - q0);
-            const long long d = d0 + c;
-            E.raw[d] = make_int4(pb, q0, k | (lg << 16), m);
-            E.key1[d] = (unsigned short)((ci << 6) | cost_bucket(wp * (double)(A.npp_prefix[q0 + k] - A.npp_prefix[q0])));
-            E.idx1[d] = (int)d;
-            if (E.raw_slot) {
+        for_chunks(A, wp, first, n, end, lane, [&](int q0, int b, unsigned peers) {
+            const int leader = __ffs(peers) - 1;
+            unsigned long long base = 0;
+            if (b >= 0 && lane == leader)
+                base = atomicAdd(&A.place[ci * kCostBuckets + b], (unsigned long long)__popc(peers));
+            base = __shfl_sync(0xffffffffu, base, leader);
+            if (b < 0) return;
+            const unsigned long long d = base + __popc(peers & ((1u << lane) - 1));
+            E.chunks[d] = make_int4(pb, q0, min(n, end - q0) | (lg << 16), m);
+            if (E.chunk_slot) {
                 // two-phase: the scratch slot of the chunk's first quartet in its (x, y, molecule)
                 // region, bra-major (the triangle q <= p for equal classes)
                 const long long *rg = &A.region[(((long long)x * kNumPairClasses + y) * S.nmol + m) * 4];
                 const long long db = pb - rg[1], dk = q0 - rg[2];
-                E.raw_slot[d] = x == y ? db * (db + 1) / 2 + dk : db * rg[3] + dk;
+                E.chunk_slot[d] = x == y ? db * (db + 1) / 2 + dk : db * rg[3] + dk;
             }
-        }
-        d0 += nc;
+        });
     });
-}
-
-__global__ void queue_place_kernel(QueueEmitArgs E) {
-    const long long d = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (d >= E.nq) return;
-    const int i = E.idx2[d];
-    E.chunks[d] = E.raw[i];
-    if (E.chunk_slot) E.chunk_slot[d] = E.raw_slot[i];
 }
 
 }  // namespace
@@ -282,37 +307,14 @@ cudaError_t plan_build_pairs(const PlanBuildArgs &A, void *temp, size_t temp_byt
     return cudaGetLastError();
 }
 
-size_t queue_count_temp_bytes(int n_items) {
-    size_t a = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, a, (long long *)nullptr, (long long *)nullptr, n_items + 1);
-    return a;
-}
-
-cudaError_t queue_count(const QueueSetup &S, const QueueArgs &A, void *temp, size_t temp_bytes,
-                        cudaStream_t s) {
-    queue_count_kernel<<<blocks_for(32LL * (A.n_items + 1)), kThreads, 0, s>>>(S, A);
-    size_t tb = temp_bytes;
-    cudaError_t e = cub::DeviceScan::ExclusiveSum(temp, tb, A.cnt, A.off, A.n_items + 1, s);
-    if (e != cudaSuccess) return e;
-    queue_summary_kernel<<<kNumClassPairs, kThreads, 0, s>>>(S, A);
+cudaError_t queue_count(const QueueSetup &S, const QueueArgs &A, cudaStream_t s) {
+    if (A.n_items > 0) queue_count_kernel<<<blocks_for(32LL * A.n_items), kThreads, 0, s>>>(S, A);
+    queue_summary_kernel<<<kNumClassPairs + 1, kThreads, 0, s>>>(S, A);
     return cudaGetLastError();
 }
 
-size_t queue_emit_temp_bytes(long long nq) {
-    size_t a = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, a, (unsigned short *)nullptr, (unsigned short *)nullptr,
-                                    (int *)nullptr, (int *)nullptr, (int)nq, 0, 13);
-    return a;
-}
-
-cudaError_t queue_emit(const QueueSetup &S, const QueueArgs &A, const QueueEmitArgs &E, void *temp,
-                       size_t temp_bytes, cudaStream_t s) {
-    if (E.nq <= 0) return cudaSuccess;
+cudaError_t queue_emit(const QueueSetup &S, const QueueArgs &A, const QueueEmitArgs &E, cudaStream_t s) {
     if (A.n_items > 0) queue_emit_kernel<<<blocks_for(32LL * A.n_items), kThreads, 0, s>>>(S, A, E);
-    size_t tb = temp_bytes;
-    cudaError_t e = cub::DeviceRadixSort::SortPairs(temp, tb, E.key1, E.key2, E.idx1, E.idx2, (int)E.nq, 0, 13, s);
-    if (e != cudaSuccess) return e;
-    queue_place_kernel<<<blocks_for(E.nq), kThreads, 0, s>>>(E);
     return cudaGetLastError();
 }
 

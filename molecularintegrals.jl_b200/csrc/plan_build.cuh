@@ -5,7 +5,7 @@
 // The reference builds its work list on the host, one shell quartet at a time
 // (eri_fetcher, src/Basis.jl:201-262); here the list is chunks of one bra pair and a run of
 // ket pairs, emitted in parallel (a warp per bra pair of each class pair) and ordered by
-// class pair and decreasing cost with a stable radix sort.
+// class pair and decreasing cost (a counting pass, then a place for each).
 #pragma once
 
 #include <cmath>
@@ -199,9 +199,9 @@ struct PlanBuildArgs {
 cudaError_t plan_build_pairs(const PlanBuildArgs &A, void *temp, size_t temp_bytes, cudaStream_t s);
 size_t plan_build_temp_bytes(int npair);
 
-// Work queues, pass 1: chunks and cost per item (bra pair of a class pair), their prefix sum,
-// and per class pair the first chunk and the total cost.  summary: kNumClassPairs + 1 chunk
-// offsets (the last one the queue length), then kNumClassPairs costs, on the device.
+// Work queues, pass 1: the chunks per (class pair, cost bucket) and the cost per item, then the first
+// place of each and the summary: kNumClassPairs + 1 chunk offsets (the last one the queue length) and
+// kNumClassPairs costs, on the device.
 struct QueueArgs {
     int n_items;
     const int *npp;                // per final pair
@@ -212,32 +212,23 @@ struct QueueArgs {
     const long long *region;       // two-phase: per (x, y, molecule) 4 fields, else null
     const double2 *bnd;            // per final pair (Qabs, R): the screening order's cut
     const double *lane_cost;       // per molecule: molecule_lane_cost
-    long long *cnt;                // n_items + 1
     double *cost;                  // n_items
-    long long *off;                // n_items + 1
+    unsigned long long *place;     // kNumClassPairs * kCostBuckets, zeroed: counts, then next places
     long long *summary;            // kNumClassPairs + 1
     double *class_cost;            // kNumClassPairs
     long long *nkept;              // kept primitive pairs
     int npair;
 };
-cudaError_t queue_count(const QueueSetup &S, const QueueArgs &A, void *temp, size_t temp_bytes,
-                        cudaStream_t s);
-size_t queue_count_temp_bytes(int n_items);
+cudaError_t queue_count(const QueueSetup &S, const QueueArgs &A, cudaStream_t s);
 
-// Work queues, pass 2: emit every chunk at its item's offset, then order the queue by class
-// pair and cost bucket (stable), writing chunks[] and, for two-phase plans, chunk_slot[].
+// Work queues, pass 2: every chunk into chunks[] (and, for two-phase plans, its slot into
+// chunk_slot[]), ordered by class pair and cost bucket.  (Listing the chunks by item first and sorting
+// them by that key took six more launches and 40 us of a 24-atom plan's creation on B200.)
 struct QueueEmitArgs {
-    int4 *raw;                     // nq
-    unsigned short *key1, *key2;   // nq
-    int *idx1, *idx2;              // nq
-    long long *raw_slot;           // nq (two-phase) or null
-    int4 *chunks;                  // nq
-    long long *chunk_slot;         // nq (two-phase) or null
-    long long nq;
+    int4 *chunks;                  // queue length
+    long long *chunk_slot;         // queue length (two-phase) or null
 };
-cudaError_t queue_emit(const QueueSetup &S, const QueueArgs &A, const QueueEmitArgs &E, void *temp,
-                       size_t temp_bytes, cudaStream_t s);
-size_t queue_emit_temp_bytes(long long nq);
+cudaError_t queue_emit(const QueueSetup &S, const QueueArgs &A, const QueueEmitArgs &E, cudaStream_t s);
 
 // Exclusive prefix sums of n ints (the gather's list positions); temp: gather_scan_temp_bytes(n).
 cudaError_t gather_scan(const int *in, int *out, long long n, void *temp, size_t temp_bytes, cudaStream_t s);
