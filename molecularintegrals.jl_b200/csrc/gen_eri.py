@@ -57,6 +57,10 @@ RYS_BOUND = {(2, 2)}
 # J/K digestion: blocks of at most this many outputs are digested from registers; larger ones sit in
 # local memory, read by a loop over A's components
 JK_UNROLL_MAX_OUT = 36
+# Resident blocks asked of the compiler where it misses a step by a few registers: (ps|ss) takes 66,
+# seven blocks of 128; eight at 64 registers: 1030 -> 1001 us over 1.17e9 integrals on B200 (the J/K
+# instantiation would spill 60 bytes for it and is left as it is)
+MIN_BLOCKS = {((1, 0), (0, 0)): 8}
 
 
 # ------------------------------------------------------------------ AO tables
@@ -363,6 +367,7 @@ def emit_class_pair(X, Y, rys=False):
         acc64.append(f"acc[{i}] = {e};")
         acc32 += [vrr_line(a, c, 0), f"acc[{i}] += (double){vname(a, c, 0)};"]
     has32 = len(entries) >= MIXED_MIN_VRR and not rys
+    bounds = f", JK ? 1 : {MIN_BLOCKS[(X, Y)]}" if (X, Y) in MIN_BLOCKS and not rys else ""
 
     def lines(x, extra=""):
         return "\n".join(f"{ind}    {extra}{ln}" for ln in x)
@@ -750,7 +755,7 @@ __device__ __forceinline__ void store_{tag}(double *__restrict__ out, const int4
 // JK: digest into J and K (molints_plan_jk) instead of storing the packed integrals; a separate
 // instantiation, so that the store kernels carry none of the digestion code.
 template <int MIXED, int JK>
-__global__ void __launch_bounds__(128) eri_queue_{tag}(const EriQueue Q) {{
+__global__ void __launch_bounds__(128{bounds}) eri_queue_{tag}(const EriQueue Q) {{
     const int lane = threadIdx.x & 31;
     for (;;) {{
         int c = 0;

@@ -176,7 +176,7 @@ __device__ __forceinline__ void jk_psss(const JKOut &jk, const int4 ib_, const i
 // JK: digest into J and K (molints_plan_jk) instead of storing the packed integrals; a separate
 // instantiation, so that the store kernels carry none of the digestion code.
 template <int MIXED, int JK>
-__global__ void __launch_bounds__(128) eri_queue_psss(const EriQueue Q) {
+__global__ void __launch_bounds__(128, JK ? 1 : 8) eri_queue_psss(const EriQueue Q) {
     const int lane = threadIdx.x & 31;
     for (;;) {
         int c = 0;
