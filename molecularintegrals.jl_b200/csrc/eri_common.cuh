@@ -120,7 +120,8 @@ __device__ __forceinline__ PrimPair load_pp(const PrimPair *__restrict__ base, i
 //                  positive, and what rounding it adds comes times d <= 1/64).  A warp's lanes read
 //                  rows at random, so every 16 bytes of a row cost about eight passes of the L1
 //                  data pipe, which was what bound the (ss|ss) and (ps|ss) kernels (78-83 % busy
-//                  with all of c_0 .. c_7 read, in 80-byte rows; the FP64 pipe 40-54 %): BOYSFIG.
+//                  with all of c_0 .. c_7 read, in 80-byte rows; the FP64 pipe 40-54 %): over 1.17e9
+//                  integrals on B200 (ss|ss) 930 -> 884 us, (ps|ps) 458 -> 409.
 //   T >= t_switch: the asymptotic family F_m = (2m-1)!! / (2T)^m * sqrt(pi/T)/2, the values
 //                  farray's Fm_asymp top order and e^-T-free recursion produce.
 // The table index is rounded with the 1.5*2^52 trick: T*32 + 1.5*2^52 holds round(T*32) in
@@ -179,7 +180,7 @@ __device__ __forceinline__ void boys_fm(double T, const BoysTab &bt, double *F) 
 // What the class kernels take: F_0..F_M at T below the switch; far (T at or above it) the asymptotic
 // family times T^(m + 1/2), (2m-1)!! / 2^m * sqrt(pi)/2 (the caller's r and r2 carry the powers of T).
 // (With the asymptotic branch of boys_fm, its own square root included, most warps ran both branches:
-// FARFIG.)
+// over 1.17e9 integrals on B200 (ss|ss) 884 us against 833, (ps|ss) 1032 against 961.)
 template <int M>
 __device__ __forceinline__ void boys_scaled(bool far, double T, const BoysTab &bt, double *F) {
     if (!far) {
