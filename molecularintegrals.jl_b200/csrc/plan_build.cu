@@ -70,17 +70,13 @@ __global__ void pair_npp_kernel(PlanBuildArgs A) {
     A.npp[k] = k < A.npair ? A.npp1[A.idx2[k]] : 0;
 }
 
-// Final pair k (the stage-1 pair idx2[k]), a warp each: its tables, with the kept primitive pairs
-// packed at npp_prefix[k], in stage-1 order.
-__global__ void pair_tables_kernel(PlanBuildArgs A) {
-    const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (k >= A.npair) return;
-    const int k1 = A.idx2[k];
+// Final pair k (the stage-1 pair k1), by a warp: its tables, with the kept primitive pairs packed at
+// `off`, in stage-1 order.
+__device__ void write_pair_tables(const PlanBuildArgs &A, int k, int k1, int off, int lane) {
     const int4 in = A.info1[k1];
     const int4 r = A.rec1[k1];
     const int2 ab = A.ab1[k1];
     const int kb = A.sh_K[ab.y];
-    const int off = (int)A.npp_prefix[k];
     const double qm = __longlong_as_double((long long)A.qmax[r.x]);
     int j = off;
     for (int x0 = 0; x0 < in.y; x0 += 32) {
@@ -105,6 +101,29 @@ __global__ void pair_tables_kernel(PlanBuildArgs A) {
         // the gather's entry of the molecule's shell pair: list position, class, A == J
         A.g_pair[A.g_mol[4 * r.x + 1] + r.y] = (k << 5) | ((r.z & 255) << 1) | (r.z >> 8);
     }
+}
+
+__global__ void pair_tables_kernel(PlanBuildArgs A) {
+    const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (k < A.npair) write_pair_tables(A, k, A.idx2[k], (int)A.npp_prefix[k], lane);
+}
+
+// Short lists: a warp per stage-1 pair counts the pairs before it, then writes its tables at its place.
+__global__ void pair_place_kernel(PlanBuildArgs A) {
+    const int k1 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (k1 >= A.npair) return;
+    const PairPlace part = pair_place(A.key1, A.npp1, A.seg1, A.npair, k1, lane, 32);
+    const int k = A.seg1[k1] + __reduce_add_sync(0xffffffffu, part.before);
+    const int off = __reduce_add_sync(0xffffffffu, part.prim), n = A.npp1[k1];
+    if (lane == 0) {
+        A.npp[k] = n;
+        A.npp_prefix[k] = off;
+        if (k == A.npair - 1) {
+            A.npp[A.npair] = 0;
+            A.npp_prefix[A.npair] = off + n;
+        }
+    }
+    write_pair_tables(A, k, k1, off, lane);
 }
 
 // ---- work queues
@@ -291,6 +310,10 @@ size_t plan_build_temp_bytes(int npair) {
 cudaError_t plan_build_pairs(const PlanBuildArgs &A, void *temp, size_t temp_bytes, cudaStream_t s) {
     if (A.npair <= 0) return cudaSuccess;
     pair_screen_kernel<<<blocks_for(32LL * A.npair), kThreads, 0, s>>>(A);
+    if (A.npair <= kPlaceMaxPairs) {
+        pair_place_kernel<<<blocks_for(32LL * A.npair), kThreads, 0, s>>>(A);
+        return cudaGetLastError();
+    }
     size_t tb = temp_bytes;
     // only the key's bits in use (a pass of the sort each 8)
     const int bits = within_bits(A.maxnpp, A.screen_sort) + bits_of((unsigned long long)(A.npair - 1));

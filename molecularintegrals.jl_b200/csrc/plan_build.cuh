@@ -146,6 +146,33 @@ struct QueueSetup {
     int zero_trunc;
 };
 
+// One lane's share of a pair's place in the final list: the pairs of its run (the stage-1 pairs with
+// the same seg) that a stable sort by key puts before it, and the kept primitive pairs of all pairs
+// before it.  Runs are contiguous and in list order, so the place is seg[k] plus the lanes' `before`.
+struct PairPlace {
+    int before, prim;
+};
+__host__ __device__ inline PairPlace pair_place(const unsigned long long *key, const int *npp, const int *seg,
+                                                int npair, int k, int lane, int lanes) {
+    PairPlace r{0, 0};
+    const int s0 = seg[k];
+    const unsigned long long mine = key[k];
+    for (int j = lane; j < s0; j += lanes) r.prim += npp[j];
+    for (int j = s0 + lane; j < npair && seg[j] == s0; j += lanes) {
+        const unsigned long long other = key[j];
+        if (other < mine || (other == mine && j < k)) {
+            ++r.before;
+            r.prim += npp[j];
+        }
+    }
+    return r;
+}
+
+// Up to this many pairs each finds its own place by counting (one launch); a longer list takes a radix
+// sort, a prefix sum and three more launches.  Plan creation on B200, counted / sorted: 55 pairs 109 /
+// 127 us, 1035 154 / 172, 2628 215 / 243; 4095 pairs in longer runs 417 / 379, 7140 716 / 519.
+constexpr int kPlaceMaxPairs = 3072;
+
 // Primitive pair x of a pair whose second shell has kb primitives: (ia << 8) | ib, A's outer.
 __host__ __device__ inline int prim_src(int x, int kb) {
     const int ia = x / kb;
