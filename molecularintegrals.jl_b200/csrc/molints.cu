@@ -132,6 +132,7 @@ struct molints_plan {
     int gather_blocks = 0;             // the context's schedule at creation: gather blocks per SM
     int sharded = 0;
     int screen_trunc = 0;              // ket runs end at the last unscreened ket (quartet screening)
+    int64_t npp_sq = 0;                // one molecule: sum of the pairs' squared kept counts
     int64_t n_zero = 0;                // pairs without kept primitive pairs (in no chunk unless sharded)
     int64_t scratch_need = 0;          // doubles of the context's scratch an execute uses: per
                                        // (class pair, molecule) a region of quartet blocks
@@ -1582,7 +1583,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     // (class-pair chunk offsets, the count of pairs without kept primitive pairs, class-pair costs,
     // kept primitive pairs, bad-shell flag)
     const size_t t_qmax = tv.take<unsigned long long>(nmol);
-    const size_t t_sum = tv.take<long long>(kNumClassPairs + 2), t_ccost = tv.take<double>(kNumClassPairs);
+    const size_t t_sum = tv.take<long long>(kNumClassPairs + 3), t_ccost = tv.take<double>(kNumClassPairs);
     const size_t t_nkept = tv.take<long long>(1), t_bad = tv.take<int>(1);
     const size_t t_place = tv.take<unsigned long long>(kNumClassPairs * kCostBuckets);
     const size_t clear_end = tv.at;
@@ -1810,6 +1811,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     QA.summary = reinterpret_cast<long long *>(tmp + t_sum);
     QA.class_cost = reinterpret_cast<double *>(tmp + t_ccost);
     QA.nkept = reinterpret_cast<long long *>(tmp + t_nkept);
+    QA.npp_sq = nmol == 1 ? reinterpret_cast<unsigned long long *>(QA.summary) + kNumClassPairs + 2 : nullptr;
     QA.npair = npair;
     if (npair > 0) {
         const double c0 = std::sqrt(2.0) * std::pow(M_PI, 1.25);
@@ -1862,6 +1864,7 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
     p->nprim_pair_kept = *reinterpret_cast<const long long *>(sum + (t_nkept - t_sum));
     const long long nq = qsum[kNumClassPairs];
     p->n_zero = qsum[kNumClassPairs + 1];
+    p->npp_sq = qsum[kNumClassPairs + 2];
     if (nq > INT32_MAX) {
         release_temp(); plan_free(p);
         return fail(ctx, MOLINTS_ERR_INVALID, "plan_create: work queue too long");
@@ -2298,7 +2301,12 @@ int molints_plan_stats(const molints_plan *p, molints_stats *st) {
     if (!p || !st) return MOLINTS_ERR_INVALID;
     if (!p->ctx) return MOLINTS_ERR_INVALID;  // its context was destroyed first
     molints_ctx *ctx = p->ctx;
-    if (int rc = plan_host_tables(p)) return rc;
+    const bool mixed = p->opts.precision == MOLINTS_MIXED && p->opts.fp32_cutoff > 0.0;
+    // one molecule without quartets to tell apart by their bounds: the counts the device summed (fetching
+    // and grouping the pair tables took 20-30 us of a drop-in call on B200)
+    const bool summed = p->nmol == 1 && !mixed && !(p->opts.screen_cutoff > 0.0);
+    if (!summed)
+        if (int rc = plan_host_tables(p)) return rc;
     std::memset(st, 0, sizeof(*st));
     st->n_eri = p->npacked;
     st->n_kernel_launches = p->n_launches;
@@ -2307,14 +2315,18 @@ int molints_plan_stats(const molints_plan *p, molints_stats *st) {
     for (int k = 0; k < 4; ++k) st->plan_ms[k] = p->plan_ms[k];
     st->n_fp32_launches = p->n_fp32_launches;
     st->n_shell_quartets += p->n_gq;
+    if (summed) {
+        const int64_t np = p->npair, sum = p->nprim_pair_kept;
+        st->n_shell_quartets += np * (np + 1) / 2;
+        st->n_prim_quartets += (sum * sum + p->npp_sq) / 2;
+    }
     // per (molecule, pair class): the pairs, gathered from the class-major list
     const int nc = kNumPairClasses;
-    std::vector<std::vector<int>> by(std::max(p->nmol, 1) * nc);
-    for (int c = 0; c < nc; ++c)
+    std::vector<std::vector<int>> by(summed ? 0 : std::max(p->nmol, 1) * nc);
+    for (int c = 0; c < nc && !summed; ++c)
         for (int k = p->class_start[c]; k < p->class_start[c + 1]; ++k) by[p->pair_mol[k] * nc + c].push_back(k);
-    const bool mixed = p->opts.precision == MOLINTS_MIXED && p->opts.fp32_cutoff > 0.0;
     const double cut = p->opts.fp32_cutoff, scut = p->opts.screen_cutoff;
-    for (int m = 0; m < p->nmol; ++m) {
+    for (int m = 0; m < p->nmol && !summed; ++m) {
         int64_t np = 0, sum = 0, sum2 = 0;
         for (int c = 0; c < nc; ++c)
             for (int k : by[m * nc + c]) { ++np; sum += p->npp_h[k]; sum2 += (int64_t)p->npp_h[k] * p->npp_h[k]; }

@@ -228,6 +228,12 @@ __global__ void queue_count_kernel(const QueueSetup S, QueueArgs A) {
 __global__ void queue_summary_kernel(const QueueSetup S, QueueArgs A) {
     const int ci = blockIdx.x;
     if (ci < kNumClassPairs) {
+        if (A.npp_sq) {
+            unsigned long long sq = 0;
+            for (int k = ci * kThreads + threadIdx.x; k < A.npair; k += kNumClassPairs * kThreads)
+                sq += (unsigned long long)A.npp[k] * A.npp[k];
+            if (sq) atomicAdd(A.npp_sq, sq);
+        }
         __shared__ double part[kThreads];
         double s = 0.0;
         for (int t = S.item_base[ci] + threadIdx.x; t < S.item_base[ci + 1]; t += blockDim.x) s += A.cost[t];

@@ -244,6 +244,7 @@ struct QueueArgs {
     long long *summary;            // kNumClassPairs + 1
     double *class_cost;            // kNumClassPairs
     long long *nkept;              // kept primitive pairs
+    unsigned long long *npp_sq;    // one-molecule plans: sum of the squared kept counts (zeroed), else null
     int npair;
 };
 cudaError_t queue_count(const QueueSetup &S, const QueueArgs &A, cudaStream_t s);
