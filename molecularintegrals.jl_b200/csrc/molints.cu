@@ -495,7 +495,7 @@ __global__ void gather_list_kernel(const int2 *__restrict__ col, const int *__re
 // Second phase of the two-phase output: the packed vector written from the scratch blocks, one
 // shell pair P at a time.  A block of threads takes the next pair from units[] (heaviest first,
 // through an atomic counter) and writes all of P's rows (function pairs ij of P), a stretch of
-// columns at a time: first the rows' stretches are cleared with 16-byte stores (not where every
+// columns at a time: first the rows' stretches are cleared by bulk copies (not where every
 // column of the stretch is computed), then each thread takes columns kl of the list of nonzero
 // columns, reads a column's descriptor once, and stores that column of every row of P with kl <= ij
 // over the zeros.  A stretch is short enough (64 KB of rows for small pairs) that its zeros are still
@@ -517,16 +517,33 @@ __global__ void gather_list_kernel(const int2 *__restrict__ col, const int *__re
 // 8-byte entry of another quartet's block.
 constexpr int kGatherMaxRows = 100;  // components of an (ff) pair
 
-// n zeros at p, by the block.
-__device__ __forceinline__ void zero_run(double *__restrict__ p, long long n) {
-    if (n <= 0) return;
-    const int head = (int)((reinterpret_cast<size_t>(p) >> 3) & 1);  // rows start at any 8-byte address
-    if (threadIdx.x == 0 && head) p[0] = 0.0;
-    double2 *__restrict__ v = reinterpret_cast<double2 *>(p + head);
-    const long long nv = (n - head) >> 1;
-    for (long long k = threadIdx.x; k < nv; k += kGatherThreads) v[k] = make_double2(0.0, 0.0);
-    if (threadIdx.x == 0 && ((n - head) & 1)) p[n - 1] = 0.0;
+// n zeros at p, by a warp whose block holds kZeroRun zeros in shared memory: bulk copies, a lane each,
+// and the odd elements at the ends by stores (rows start at any 8-byte address, bulk copies at
+// multiples of 16).  The warp's threads wait for them with zero_wait.
+constexpr int kZeroRun = 256;
+
+// The block's zeros, to be followed by a barrier of its threads.
+__device__ __forceinline__ void zero_fill(double *zeros, int threads) {
+    for (int k = threadIdx.x; k < kZeroRun; k += threads) zeros[k] = 0.0;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
+
+__device__ __forceinline__ void zero_run(double *__restrict__ p, long long n, const double *zeros, int lane) {
+    if (n <= 0) return;
+    const int head = (int)((reinterpret_cast<size_t>(p) >> 3) & 1);
+    const long long body = (n - head) & ~1LL;
+    if (lane == 0 && head) p[0] = 0.0;
+    if (lane == 0 && head + body < n) p[n - 1] = 0.0;
+    const unsigned src = (unsigned)__cvta_generic_to_shared(zeros);
+    for (long long k = (long long)lane * kZeroRun; k < body; k += 32 * kZeroRun)
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(
+                         __cvta_generic_to_global(p + head + k)),
+                     "r"(src), "r"((int)min((long long)kZeroRun, body - k) * 8)
+                     : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+
+__device__ __forceinline__ void zero_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // The listed columns [j0, j1) of one shell pair P for the gather: NC columns per thread and pass,
 // their descriptor loads first, then the scratch loads of NR rows of each column (NC * NR in
@@ -640,20 +657,28 @@ struct GatherArgs {
     double screen_cut;
 };
 
-// The rows of the units that are all zeros: contiguous runs, at DRAM's write rate (5.1 GB in 0.83 ms).
-// Nothing else writes them, so this kernel runs beside the class kernels, which leave DRAM idle, with
-// two blocks per SM (execute of 1.17e9 integrals, FP64 / screened, with 1, 1.5, 2, 3 and 4 blocks
-// per SM: 6.87 / 5.16, 6.79 / 4.92, 6.84 / 4.88, 6.96 / 5.07, 7.07 / 5.20 ms).
-__global__ void __launch_bounds__(kGatherThreads) zero_rows_kernel(const GatherArgs A) {
-    __shared__ int s_unit;
+// The rows of the units that are all zeros, contiguous runs that nothing else writes, so this kernel
+// runs beside the class kernels, which leave DRAM idle: single warps that copy zeros out of shared
+// memory, so that they take few registers and no issue slots from those.  A warp's copies are starved
+// by the class kernels' own shared-memory and L1 traffic, hence eight per SM.  Execute of 1.17e9
+// integrals (5.1 GB of such rows; 0.72 ms alone) on B200, FP64 / screened: without these rows 5.48 /
+// 3.53 ms; 16-byte stores by two blocks of 256 threads per SM 6.23 / 4.48; bulk copies by 1, 2, 4, 8,
+// 12 and 16 warps per SM 8.1 / 7.4, 6.43 / 5.51, 6.13 / 4.61, 5.99 / 4.18, 5.98 / 4.15, 6.05 / 4.19
+// (16 KB a copy instead of 2: fewer blocks find room beside the class kernels', 6.59 / 6.35 with two).
+constexpr int kZeroBlocks = 8;  // warps per SM
+
+__global__ void __launch_bounds__(32) zero_rows_kernel(const GatherArgs A) {
+    __shared__ __align__(16) double zeros[kZeroRun];
+    const int lane = threadIdx.x;
+    zero_fill(zeros, 32);
+    __syncwarp();
     const long long first = __ldg(A.n_live);
     for (;;) {
-        __syncthreads();
-        if (threadIdx.x == 0) s_unit = atomicAdd(A.counter + 1, 1);
-        __syncthreads();
+        int k = 0;
+        if (lane == 0) k = atomicAdd(A.counter + 1, 1);
         // the list's end holds the heavy units
-        const long long u = A.nunits - 1 - s_unit;
-        if (u < first) return;
+        const long long u = A.nunits - 1 - __shfl_sync(0xffffffffu, k, 0);
+        if (u < first) break;
         const int4 un = __ldg(&A.units[u]);
         const int nI = un.w & 255, nJ = (un.w >> 8) & 255, same = (un.w >> 16) & 1;
         double *__restrict__ obase = A.out + __ldg(&A.mol[4 * un.x + 2]);
@@ -661,10 +686,12 @@ __global__ void __launch_bounds__(kGatherThreads) zero_rows_kernel(const GatherA
             const long long i = un.y + a;
             for (int b = 0; b < (same ? a + 1 : nJ); ++b) {
                 const long long ij = i * (i + 1) / 2 + un.z + b;
-                zero_run(obase + ij * (ij + 1) / 2, ij + 1);
+                zero_run(obase + ij * (ij + 1) / 2, ij + 1, zeros, lane);
+                asm volatile("cp.async.bulk.wait_group.read 4;" ::: "memory");  // (a bound on those in flight)
             }
         }
     }
+    zero_wait();
 }
 
 __global__ void __launch_bounds__(kGatherThreads) gather_packed_kernel(const GatherArgs A) {
@@ -674,6 +701,8 @@ __global__ void __launch_bounds__(kGatherThreads) gather_packed_kernel(const Gat
     __shared__ long long s_ij[kGatherMaxRows], s_tri[kGatherMaxRows];
     __shared__ int s_rc[kGatherMaxRows];
     __shared__ long long s_unit;
+    __shared__ __align__(16) double zeros[kZeroRun];
+    zero_fill(zeros, kGatherThreads);
     const double screen_cut = A.screen_cut;
     for (;;) {
         __syncthreads();  // the previous unit's readers are done with the shared tables
@@ -723,7 +752,9 @@ __global__ void __launch_bounds__(kGatherThreads) gather_packed_kernel(const Gat
             const int j0 = __ldg(&index[c0 >> kGatherIndexShift]);
             const int j1 = c1 < nrowsM ? __ldg(&index[c1 >> kGatherIndexShift]) : __ldg(&A.end[m]);
             if (screen_cut > 0.0 || j1 - j0 < min(c1, nrowsM) - c0) {
-                for (int r = 0; r < R; ++r) zero_run(obase + s_tri[r] + c0, min(c1, s_ij[r] + 1) - c0);
+                for (int r = threadIdx.x >> 5; r < R; r += kGatherThreads / 32)
+                    zero_run(obase + s_tri[r] + c0, min(c1, s_ij[r] + 1) - c0, zeros, threadIdx.x & 31);
+                zero_wait();
                 __syncthreads();  // the zeros come before the entries
             }
             // pairs of one or a few rows (ss, sp) are most of the units: their copies have no row loop
@@ -2035,7 +2066,7 @@ static int plan_enqueue(molints_plan *p, double *out_device, bool timing, JKOut 
         // the all-zero rows, on a stream of their own until the end of the execute
         if (nside) MI_CUDA(ctx, cudaStreamWaitEvent(zs, ctx->fork, 0));
         if (int rc = mark(launches, "zero_rows", 0, zs)) return rc;
-        zero_rows_kernel<<<(int)std::min<int64_t>(2 * ctx->num_sms, p->n_units), kGatherThreads, 0, zs>>>(G);
+        zero_rows_kernel<<<(int)std::min<int64_t>(kZeroBlocks * ctx->num_sms, p->n_units), 32, 0, zs>>>(G);
         if (int rc = mark(launches, "zero_rows", 1, zs)) return rc;
         ++launches;
         if (nside) MI_CUDA(ctx, cudaEventRecord(ctx->join[molints_ctx::kSideTwoPhase], zs));
