@@ -435,8 +435,9 @@ def profile_pass(plans, out):
 def measure_roofline(plans, groups, mols, out, stream, dev):
     """One serialised profiling pass of the FP64 plans (per-launch CUDA events on the launching
     stream), per kernel its device time over the whole batch.  The dominant kernel gets the
-    roofline: the gather pass of the two-phase output is HBM-bound (16 algorithmic bytes per
-    packed integral: one scratch read, one output write; peak = MEASURED_PEAKS.json hbm_gbs),
+    roofline: the gather pass of the two-phase output and the rows it leaves to zero_rows are
+    HBM-bound together (8 algorithmic bytes per packed integral, its output write; the scratch
+    reads, of the nonzero quartets alone, are not counted; peak = MEASURED_PEAKS.json hbm_gbs),
     a class kernel FP64-bound (flops.py algorithmic FLOP over all primitive quartets; peak =
     FP64 DGEMM measured here).  The top class kernel is reported beside it, also against the
     FLOP of the primitive quartets it evaluates (after primitive-pair screening).  DRAM
@@ -475,11 +476,12 @@ def measure_roofline(plans, groups, mols, out, stream, dev):
     top_cls = max(cls, key=times.get)
     top = max(times, key=times.get)
     if top == "gather_packed":
-        ach = 16.0 * n_eri / (times[top] * 1e-3) / 1e9
+        both = times[top] + times.get("zero_rows", 0.0)
+        ach = 8.0 * n_eri / (both * 1e-3) / 1e9
         t = traffic_db.get(top)
-        roof = {"bound": "hbm", "kernel": top, "achieved": ach, "peak": hbm, "unit": "GB/s",
-                "frac": ach / hbm, "launches": nlaunch[top], "kernel_ms_per_step": times[top],
-                "algorithmic_bytes_per_step": 16.0 * n_eri,
+        roof = {"bound": "hbm", "kernel": top + " + zero_rows", "achieved": ach, "peak": hbm, "unit": "GB/s",
+                "frac": ach / hbm, "launches": nlaunch[top] + nlaunch.get("zero_rows", 0),
+                "kernel_ms_per_step": both, "algorithmic_bytes_per_step": 8.0 * n_eri,
                 "traffic": None if t is None else t * n_eri / nlaunch[top], "peak_source": hbm_src}
     else:
         roof = class_entry(top)

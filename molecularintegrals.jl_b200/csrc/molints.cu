@@ -2,11 +2,14 @@
 // include/molints.h, plus the device pair builder and the Boys-table kernels.
 //
 // Execution of a plan (all on the context's stream, no host synchronisation):
-//   1. build_pairs_kernel: one thread per canonical shell pair writes its primitive-pair
-//      records (zeta, P, P-A, exp(-ab/zeta |A-B|^2) prefactor) and A-B;
-//   2. schwarz kernels, one per pair class: Q_p = sqrt(max |(ab|ab)|);
-//   3. one generated kernel per class pair (bra class >= ket class) over all its unique
-//      shell quartets, writing the packed iindex vector.
+//   1. build_pairs_kernel writes the primitive-pair records (zeta, P, P-A, prefactor) and A-B of the
+//      listed shell pairs; a large direct output is cleared beside it;
+//   2. one generated kernel per class pair (bra class >= ket class) over its work queue, and the
+//      generic kernel for quartets with a g shell, into the packed iindex vector;
+//   3. or, for large outputs, into a scratch of quartet blocks, from which the gather writes the
+//      packed vector (its all-zero rows beside the class kernels).
+// Plan creation (pair list on the host; bounds, screening, tables and queues on the device) is in
+// plan_create_impl and plan_build.cu.
 // The drivers this replaces are all_twoe_ints_chrr (src/HGP.jl:22-34) and all_twoe_ints
 // (src/ERI.jl:104-112) of MolecularIntegrals.jl.
 #include <cuda_runtime.h>
@@ -2126,7 +2129,7 @@ static int plan_enqueue(molints_plan *p, double *out_device, bool timing, JKOut 
         // second phase: the packed vector in order from the scratch blocks
         if (int rc = mark(launches, "gather_packed", 0, s)) return rc;
         // a persistent grid of gather_blocks blocks per SM; blocks beyond what the kernel's
-        // registers let reside (five at 44 registers) start as others finish, and find the
+        // registers let reside (four at 64 registers) start as others finish, and find the
         // unit list done
         const int gb = p->gather_blocks > 0 ? p->gather_blocks : kGatherBlocksDefault;
         const int grid = (int)std::min<long long>((long long)ctx->num_sms * gb, p->n_units);
