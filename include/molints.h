@@ -68,7 +68,7 @@ enum molints_output { MOLINTS_OUTPUT_AUTO = 0, MOLINTS_OUTPUT_DIRECT = 1, MOLINT
 /* Largest shell angular momentum the engine accepts (g = 4), as the reference's tables
  * (shell_indices, src/Basis.jl:269-279).  Class pairs up to (ff|ff) run the generated HGP or Rys
  * kernels (n <= 7 roots); every shell quartet with a g shell runs one generic Rys kernel (n <= 9
- * roots, FP64, no screening), written for coverage rather than speed.  Plans with a g shell use
+ * roots, FP64, no screening).  Plans with a g shell use
  * the direct output and support neither sharding, J/K digestion nor molints_plan_schwarz
  * (MOLINTS_ERR_UNSUPPORTED). */
 #define MOLINTS_LMAX 4
