@@ -148,30 +148,34 @@ struct QueueSetup {
 
 // One lane's share of a pair's place in the final list: the pairs of its run (the stage-1 pairs with
 // the same seg) that a stable sort by key puts before it, and the kept primitive pairs of all pairs
-// before it.  Runs are contiguous and in list order, so the place is seg[k] plus the lanes' `before`.
+// before it.  Runs are contiguous, in list order and in the key's high bits, so the place is seg[k] plus
+// the lanes' `before`.  Every pair is looked at, not only those up to the run's end: independent loads,
+// several in flight (a loop that ended with the run took 27 us on 2628 pairs on B200, and
+// plan creation 213 us; so 197).
 struct PairPlace {
     int before, prim;
 };
 __host__ __device__ inline PairPlace pair_place(const unsigned long long *key, const int *npp, const int *seg,
                                                 int npair, int k, int lane, int lanes) {
-    PairPlace r{0, 0};
     const int s0 = seg[k];
     const unsigned long long mine = key[k];
-    for (int j = lane; j < s0; j += lanes) r.prim += npp[j];
-    for (int j = s0 + lane; j < npair && seg[j] == s0; j += lanes) {
+    PairPlace r{lane < s0 ? -((s0 - lane + lanes - 1) / lanes) : 0, 0};  // (less the lane's pairs of earlier runs)
+#pragma unroll 8
+    for (int j = lane; j < npair; j += lanes) {
         const unsigned long long other = key[j];
-        if (other < mine || (other == mine && j < k)) {
-            ++r.before;
-            r.prim += npp[j];
-        }
+        const int n = npp[j];
+        const bool ahead = other < mine || (other == mine && j < k);
+        r.before += ahead;
+        r.prim += ahead ? n : 0;
     }
     return r;
 }
 
-// Up to this many pairs each finds its own place by counting (one launch); a longer list takes a radix
-// sort, a prefix sum and three more launches.  Plan creation on B200, counted / sorted: 55 pairs 109 /
-// 127 us, 1035 154 / 172, 2628 215 / 243; 4095 pairs in longer runs 417 / 379, 7140 716 / 519.
-constexpr int kPlaceMaxPairs = 3072;
+// Up to this many pairs each finds its own place by counting (one launch, n^2 / 32 steps of a warp); a
+// longer list takes a radix sort, a prefix sum and three more launches.  Plan creation on B200, counted
+// / sorted: 55 pairs 103 / 127 us, 1035 146 / 172, 2628 197 / 243, 4095 342 / 373, 4656 393 / 415, 7140
+// 505 / 508, 16290 1095 / 958.
+constexpr int kPlaceMaxPairs = 6144;
 
 // Primitive pair x of a pair whose second shell has kb primitives: (ia << 8) | ib, A's outer.
 __host__ __device__ inline int prim_src(int x, int kb) {
