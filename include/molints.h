@@ -46,7 +46,10 @@ enum molints_method { MOLINTS_METHOD_AUTO = 0, MOLINTS_METHOD_HGP = 1, MOLINTS_M
 enum molints_precision { MOLINTS_FP64 = 0, MOLINTS_MIXED = 1 };
 enum molints_boys {
     /* farray of src/Boys.jl:19-27: exact F_m below T = 30, the asymptotic form (without the
-     * e^-T terms) from T = 30 up.  Matches the reference HGP bit for bit up to rounding. */
+     * e^-T terms) from T = 30 up.  What the HGP kernels evaluate, and under AUTO the Rys kernels of
+     * (dp|pp), (dp|ds), (fs|dp), (fs|fs), (dd|ps), (dd|pp), (dd|ds), (dd|dp), (fp|ds) and (fd|ps):
+     * there it matches the reference HGP up to rounding.  The other Rys kernels evaluate the exact
+     * F_m in either mode. */
     MOLINTS_BOYS_REFERENCE = 0,
     /* exact F_m (table + Taylor + downward recursion) up to T = 40, asymptotic beyond. */
     MOLINTS_BOYS_EXACT = 1
@@ -94,8 +97,8 @@ typedef struct molints_basis {
 typedef struct molints_options {
     int32_t method;          /* enum molints_method */
     int32_t precision;       /* enum molints_precision */
-    int32_t boys;            /* enum molints_boys; the Rys kernels always evaluate the exact
-                                quadrature (there is no T >= 30 branch to follow) */
+    int32_t boys;            /* enum molints_boys; METHOD_RYS evaluates the exact quadrature in
+                                either mode */
     int32_t output;          /* enum molints_output */
     /* Both cutoffs compare against B = Qabs_ab * Qabs_cd, where Qabs_ab is the sum over the
      * pair's primitive pairs i of sqrt(max |(a_i b_i|a_i b_i)|).  B bounds the sum of the

@@ -948,7 +948,8 @@ def emit_dispatch(pairs):
 def emit_class_table(path: Path):
     """class_table.h: the default per-class-pair method table of MOLINTS_METHOD_AUTO, from the
     class tuner's result kept in data/class_table_<gpu>.json (the classes it found faster with
-    Rys, and those whose FP32 variant it found faster than FP64)."""
+    Rys, those of them whose Rys kernel follows the Boys mode under AUTO, and those whose FP32 variant
+    it found faster than FP64)."""
     import json
     d = json.loads(path.read_text())
     cls = gen_rys.pair_classes()
@@ -976,6 +977,15 @@ def emit_class_table(path: Path):
              f"static const int32_t kTunedClassMethods[{n}][{n}] = {{"]
     for x in range(n):
         lines.append("    {" + ", ".join(str(v) for v in tab[x]) + "},")
+    follow = {idx(t) for t in d["follow_boys"]}
+    lines += ["};",
+              "// 1 where an AUTO plan's Rys kernel follows the Boys mode as the HGP kernel of the class pair does",
+              "// (RysTab::xmax = 30 in the reference mode): (dp|dp), (fp|pp) and (dd|dd) evaluate the exact function",
+              "// in either mode, and so do the class pairs without an HGP kernel.  For nine polarised atoms with f",
+              "// shells the two forms differ by up to 7.4e-12 in (dd|pp), 1.3e-12 in (dd|ps).",
+              f"static const unsigned char kRysFollowsBoys[{n}][{n}] = {{"]
+    for x in range(n):
+        lines.append("    {" + ", ".join(str(int((x, y) in follow)) for y in range(n)) + "},")
     # work-queue schedule (molints_schedule: lane_cost, hgp_widen, rys_chunks, rys_max_width,
     # gather_blocks), the built-in values where the tuner's result has none
     sc = dict({"lane_cost": 80.0, "hgp_widen": 1, "rys_chunks": 4096, "rys_max_width": 8, "gather_blocks": 5},

@@ -107,6 +107,7 @@ struct molints_plan {
     double class_cost[kNumPairClasses][kNumPairClasses] = {};  // kept primitive quartets
     int method[kNumPairClasses][kNumPairClasses] = {};  // MOLINTS_METHOD_HGP or _RYS
     int fp32[kNumPairClasses][kNumPairClasses] = {};    // MIXED and this class's FP32 variant used
+    bool rys_mode[kNumPairClasses][kNumPairClasses] = {};  // the Rys kernel takes the reference mode's form
     // host copies (final, screened order): pair_mol from plan creation (the re-sort by kept
     // count stays within each molecule's run), the rest fetched on first use (plan_host_tables)
     std::vector<int> pair_mol;         // canonical pair -> molecule
@@ -1321,6 +1322,8 @@ static int plan_create_impl(molints_ctx *ctx, int32_t nmol, const molints_basis 
             if (m == MOLINTS_METHOD_AUTO) m = MOLINTS_METHOD_HGP;
             if (!kEriLaunchers[x][y]) m = MOLINTS_METHOD_RYS;
             p->method[x][y] = m;
+            p->rys_mode[x][y] = m == MOLINTS_METHOD_RYS && opts.method == MOLINTS_METHOD_AUTO &&
+                                opts.boys == MOLINTS_BOYS_REFERENCE && kRysFollowsBoys[x][y];
             // MIXED plans run this class's FP32 variant where the chosen kernel has one, unless
             // the table measured that kernel's FP32 variant no faster (the flag speaks for the
             // table's own method only)
@@ -2115,7 +2118,9 @@ static int plan_enqueue(molints_plan *p, double *out_device, bool timing, JKOut 
                              : (int)std::min<long long>((long long)occ * ctx->num_sms, (Q.nchunks + 3) / 4);
         const char *name = rys ? kRysNames[x][y] : kEriNames[x][y];
         if (int rc = mark(launches, name, 0, st)) return rc;
-        if (rys) kRysLaunchers[x][y](Q, ctx->rys, mixed, grid, st);
+        RysTab R = ctx->rys;
+        if (p->rys_mode[x][y]) R.xmax = kBoysReferenceSwitch;
+        if (rys) kRysLaunchers[x][y](Q, R, mixed, grid, st);
         else kEriLaunchers[x][y](Q, mixed, grid, st);
         fp32_launches += mixed;
         if (int rc = mark(launches, name, 1, st)) return rc;

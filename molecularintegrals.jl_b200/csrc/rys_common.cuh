@@ -30,7 +30,7 @@
 
 namespace molints {
 
-constexpr int kRysXmax = 100;   // Chebyshev fits on [0, 100); Gauss-Hermite limit above
+constexpr int kRysXmax = 100;   // Chebyshev fits on [0, 100)
 constexpr int kRysNcheb = 16;
 
 // Class tables emitted by gen_rys.py.
@@ -64,11 +64,11 @@ __device__ __forceinline__ double clenshaw16(const double *__restrict__ c, doubl
     return fma(s, b1, q[0].x - b2);
 }
 
-// Node u_r = t_r^2 and weight W_r of the NR-point Rys rule at X >= 0:
-// sum_r W_r u_r^m = F_m(X) for m < 2 NR.
+// Node u_r = t_r^2 and weight W_r of the NR-point Rys rule at X >= 0: sum_r W_r u_r^m = F_m(X) for
+// m < 2 NR, from X = R.xmax on the asymptotic form of F_m (Gauss-Hermite limit).
 template <int NR>
 __device__ __forceinline__ void rys_root(const RysTab &R, double X, int r, double &u, double &w) {
-    if (X < (double)kRysXmax) {
+    if (X < R.xmax) {
         const int j = (int)X;
         const double s = 2.0 * (X - (double)j) - 1.0;
         const double *c = R.cheb + (size_t)kRysXmax * kRysNcheb * NR * (NR - 1) +
