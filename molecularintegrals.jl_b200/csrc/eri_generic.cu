@@ -47,7 +47,7 @@ constexpr int kGenL = 4;                          // highest shell angular momen
 constexpr int kGenE = 2 * kGenL;                  // la + lb
 constexpr int kGenRysXmax = 100;
 constexpr int kGenNcheb = 16;
-constexpr int kGenItems = 96;                     // (primitive quartet, root) items set up at once
+constexpr int kGenItems = 96;                     // (primitive quartet, root) items set up at once, at most
 // doubles of each of the two table regions (H and I): the 1-D tables of three (gg|gg) items
 // (3 * 5^4 doubles each), more items of smaller quartets.  Two blocks per SM.
 constexpr int kGenRegion = 5760;
@@ -172,20 +172,18 @@ __global__ void __launch_bounds__(kGenThreads, 2) eri_generic_kernel(const GenQu
             const int ab = o < tn ? (t0 + o) / ncd : 0, cd = o < tn ? t0 + o - ab * ncd : 0;
             off[j] = sOff[0][ab] + sOff[1][cd];
         }
-        const int nitem = np[0] * np[1] * np[2] * np[3] * nr;
+        const unsigned nquart = gen_prim_count(np);
+        const int per = kGenItems / nr;  // primitive quartets set up at once
         const int batch = min(kGenBatch, kGenRegion / (3 * IS));  // HS <= IS
-        for (int g0 = 0; g0 < nitem; g0 += kGenItems) {
-            const int ng = min(kGenItems, nitem - g0);
+        for (unsigned g0 = 0; g0 < nquart; g0 += per) {
+            const int ng = (int)min((unsigned)per, nquart - g0) * nr;
             if (tid < ng) {
-                // item: primitive quartet (the last shell's primitive fastest) and root.  The previous
-                // items' readers (the H phase) are done: a barrier follows every H phase.
-                int pq = (g0 + tid) / nr;
-                const int r = g0 + tid - pq * nr;
-                const int pd = pq % np[3]; pq /= np[3];
-                const int pc = pq % np[2]; pq /= np[2];
-                const int pb = pq % np[1], pa = pq / np[1];
-                const double a = __ldg(&Gq.expn[po[0] + pa]), b = __ldg(&Gq.expn[po[1] + pb]);
-                const double c = __ldg(&Gq.expn[po[2] + pc]), d = __ldg(&Gq.expn[po[3] + pd]);
+                // item: primitive quartet and root.  The previous items' readers (the H phase) are done:
+                // a barrier follows every H phase.
+                const int pq = tid / nr, r = tid - pq * nr;
+                const GenPrims k4 = gen_prim(g0 + pq, np);
+                const double a = __ldg(&Gq.expn[po[0] + k4.a]), b = __ldg(&Gq.expn[po[1] + k4.b]);
+                const double c = __ldg(&Gq.expn[po[2] + k4.c]), d = __ldg(&Gq.expn[po[3] + k4.d]);
                 const double z = a + b, e = c + d, ze = z + e;
                 double ab2 = 0.0, cd2 = 0.0, pq2 = 0.0, PA[3], QC[3], QP[3];
 #pragma unroll
@@ -200,8 +198,8 @@ __global__ void __launch_bounds__(kGenThreads, 2) eri_generic_kernel(const GenQu
                     QP[k] = Q - P;
                     pq2 += (P - Q) * (P - Q);
                 }
-                const double coef = __ldg(&Gq.ncoef[po[0] + pa]) * __ldg(&Gq.ncoef[po[1] + pb]) *
-                                    __ldg(&Gq.ncoef[po[2] + pc]) * __ldg(&Gq.ncoef[po[3] + pd]);
+                const double coef = __ldg(&Gq.ncoef[po[0] + k4.a]) * __ldg(&Gq.ncoef[po[1] + k4.b]) *
+                                    __ldg(&Gq.ncoef[po[2] + k4.c]) * __ldg(&Gq.ncoef[po[3] + k4.d]);
                 const double pref = 2.0 * 17.493418327624862 /* pi^2.5 */ / (z * e * sqrt(ze)) *
                                     exp(-a * b / z * ab2 - c * d / e * cd2) * coef;
                 double u, w;
