@@ -184,11 +184,20 @@ struct RysPart {
     }
 };
 
+// Primitive quartets of a quartet whose pairs keep nb and nk primitive pairs.  Unsigned: shells have up to
+// 255 primitives, and 255^4 + 128 (a kernel's step) is below 2^32 where 216^4 is above 2^31.
+__host__ __device__ __forceinline__ unsigned rys_prim_count(int nb, int nk) { return (unsigned)nb * (unsigned)nk; }
+
+// Of a quartet of nq primitive quartets, those in the batch of pb that starts at g0.
+__host__ __device__ __forceinline__ int rys_batch(unsigned nq, unsigned g0, int pb) {
+    return nq > g0 ? (int)(nq - g0 < (unsigned)pb ? nq - g0 : (unsigned)pb) : 0;
+}
+
 // One round's ket pairs as a thread sees them.
 struct RysKets {
-    int kx;         // stage 1: first ket primitive pair of w1
-    int nq1, nq2;   // primitive quartets of w1's and of w2's quartet (0: none, or no part)
-    int nqmax;      // the round's largest count, the same in every thread of the group
+    int kx;              // stage 1: first ket primitive pair of w1
+    unsigned nq1, nq2;   // primitive quartets of w1's and of w2's quartet (0: none, or no part)
+    unsigned nqmax;      // the round's largest count, the same in every thread of the group
     bool f1, f2;    // MIXED: w1's / w2's quartet below the FP32 cutoff
 };
 
@@ -204,17 +213,17 @@ __device__ __forceinline__ void rys_contract(const PairTab &P, const RysTab &R, 
     constexpr int S = C::S, F1 = C::F + 1, NR = C::NR, E = C::E, NA = C::NA, PB = C::PB, SI = C::SI;
 #pragma unroll
     for (int a = 0; a < NA; ++a) acc[a] = 0.0;
-    for (int g0 = 0; g0 < K.nqmax; g0 += PB) {
+    for (unsigned g0 = 0; g0 < K.nqmax; g0 += PB) {
         if (g0 + L.b1 < K.nq1) {
-            const int g = g0 + L.b1, gj = g / nbp;
-            const PrimPair bra = load_pp(P.pp, bx + (g - gj * nbp));
-            const PrimPair ket = load_pp(P.pp, K.kx + gj);
+            const unsigned g = g0 + L.b1, gj = g / (unsigned)nbp;
+            const PrimPair bra = load_pp(P.pp, bx + (int)(g - gj * nbp));
+            const PrimPair ket = load_pp(P.pp, K.kx + (int)gj);
             double *tab = work + ((L.w1 * PB + L.b1) * NR + L.r1) * SI;
             if (MIXED && K.f1) rys_tables_of<C, float>(R, bra, ket, L.r1, reinterpret_cast<float *>(tab));
             else rys_tables_of<C, double>(R, bra, ket, L.r1, tab);
         }
         group_sync<C::G>(gid);
-        const int ni = min(PB, K.nq2 - g0) * NR;  // this quartet's (primitive quartet, root) items
+        const int ni = rys_batch(K.nq2, g0, PB) * NR;  // this quartet's (primitive quartet, root) items
         const double *__restrict__ t0 = work + L.w2 * PB * NR * SI;
         if (MIXED && K.f2) {
             float bacc[NA];
@@ -378,7 +387,7 @@ __device__ __forceinline__ void rys_queue_body(const EriQueue &Q, const RysTab &
                 const int4 ik = __ldg(&Q.pairs.info[q]);
                 const double2 bq = __ldg(&Q.pairs.bnd[q]);
                 K.kx = ik.x;
-                K.nq1 = (bp.x * bq.x < Q.screen_cut) ? 0 : ib.y * ik.y;  // screened: written as 0
+                K.nq1 = (bp.x * bq.x < Q.screen_cut) ? 0 : rys_prim_count(ib.y, ik.y);  // screened: written as 0
                 K.f1 = MIXED && bp.y * bq.y < Q.fp32_cut;
             }
             if constexpr (C::W == 1) {
@@ -391,7 +400,7 @@ __device__ __forceinline__ void rys_queue_body(const EriQueue &Q, const RysTab &
                     const int q = q0 + L.w2;
                     const int4 ik = __ldg(&Q.pairs.info[q]);
                     const double2 bq = __ldg(&Q.pairs.bnd[q]);
-                    K.nq2 = (bp.x * bq.x < Q.screen_cut) ? 0 : ib.y * ik.y;
+                    K.nq2 = (bp.x * bq.x < Q.screen_cut) ? 0 : rys_prim_count(ib.y, ik.y);
                     K.f2 = MIXED && bp.y * bq.y < Q.fp32_cut;
                 }
                 K.nqmax = __reduce_max_sync(0xffffffffu, K.nq1);
@@ -452,7 +461,8 @@ __device__ __forceinline__ void rys_bound_body(const PairTab &P, const RysTab &R
     double q = 0.0;  // sum of b_k in list order
     for (int k = 0; k < nk; ++k) {
         const int i0 = full ? 0 : k, n = full ? in.y : 1;
-        const RysKets K{in.x + i0, L.w1 == 0 ? n * n : 0, L.w2 == 0 ? n * n : 0, n * n, false, false};
+        const unsigned nq = rys_prim_count(n, n);
+        const RysKets K{in.x + i0, L.w1 == 0 ? nq : 0, L.w2 == 0 ? nq : 0, nq, false, false};
         double acc[C::NA];
         rys_contract<C, 0>(P, R, L, in.x + i0, n, K, work, acc, gid);
         double wmax = 0.0, m = 0.0;

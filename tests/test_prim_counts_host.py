@@ -50,3 +50,39 @@ def _run(program, tmp_path):
 
 def test_generic_kernel(tmp_path):
     _run(GENERIC, tmp_path)
+
+
+RYS = r"""
+#include <cstdio>
+#include <initializer_list>
+#include "rys_common.cuh"
+using namespace molints;
+int main() {
+    int bad = 0;
+    const unsigned long long top = 255ull * 255;
+    for (unsigned long long nb : {1ull, 7ull, 216ull * 216, top})
+        for (unsigned long long nk : {1ull, 49ull, 216ull * 216, top}) {
+            const unsigned n = rys_prim_count((int)nb, (int)nk);
+            bad += n != nb * nk || nb * nk + 128 > 0xffffffffull;
+        }
+    // the batches of a quartet of nq primitive quartets, in a round that goes on for a longer one
+    for (unsigned nq : {0u, 1u, 31u, 32u, 33u, 100u})
+        for (int pb : {1, 7, 32, 128}) {
+            unsigned sum = 0;
+            for (unsigned g0 = 0; g0 < 300; g0 += pb) {
+                const int n = rys_batch(nq, g0, pb);
+                bad += n < 0 || n > pb;
+                sum += n;
+            }
+            bad += sum != nq;
+        }
+    const unsigned big = rys_prim_count((int)top, (int)top);
+    bad += rys_batch(big, 0, 32) != 32 || rys_batch(big, big - 5, 32) != 5 || rys_batch(big, big, 32) != 0;
+    std::printf("%d\n", bad);
+    return bad != 0;
+}
+"""
+
+
+def test_rys_kernels(tmp_path):
+    _run(RYS, tmp_path)
