@@ -88,7 +88,6 @@ void launch_rys_ppps(const EriQueue &Q, const RysTab &R, int mixed, int grid, cu
 int occupancy_rys_ppps(int mixed);
 void launch_rys_pppp(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_pppp(int mixed);
-void launch_rys_bound_pppp(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s);
 void launch_rys_dsss(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_dsss(int mixed);
 void launch_rys_dsps(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
@@ -97,7 +96,6 @@ void launch_rys_dspp(const EriQueue &Q, const RysTab &R, int mixed, int grid, cu
 int occupancy_rys_dspp(int mixed);
 void launch_rys_dsds(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_dsds(int mixed);
-void launch_rys_bound_dsds(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s);
 void launch_rys_dpss(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_dpss(int mixed);
 void launch_rys_dpps(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
@@ -108,7 +106,6 @@ void launch_rys_dpds(const EriQueue &Q, const RysTab &R, int mixed, int grid, cu
 int occupancy_rys_dpds(int mixed);
 void launch_rys_dpdp(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_dpdp(int mixed);
-void launch_rys_bound_dpdp(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s);
 void launch_rys_fsss(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_fsss(int mixed);
 void launch_rys_fsps(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
@@ -121,7 +118,6 @@ void launch_rys_fsdp(const EriQueue &Q, const RysTab &R, int mixed, int grid, cu
 int occupancy_rys_fsdp(int mixed);
 void launch_rys_fsfs(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_fsfs(int mixed);
-void launch_rys_bound_fsfs(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s);
 void launch_rys_ddss(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
 int occupancy_rys_ddss(int mixed);
 void launch_rys_ddps(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);
@@ -300,7 +296,7 @@ static const float kRysPrimCost[11][11] = {
     {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f},
 };
 // 1 where the class pair's kernel has an FP32 variant for MIXED quartets (HGP: at least
-// 40 VRR entries; Rys: gen_rys's MIXED_MIN_NBLK / MIXED_MAX_ACC rule), else 0
+// 40 VRR entries; Rys: 32 to 3072 block entries), else 0
 static const unsigned char kEriHasFp32[11][11] = {
     {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0},
     {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0},
@@ -373,6 +369,6 @@ static const SchwarzLauncher kSchwarzLaunchers[11] = {
     launch_schwarz_ssss, launch_schwarz_psps, launch_schwarz_pppp, launch_schwarz_dsds, launch_schwarz_dpdp, launch_schwarz_fsfs, nullptr, nullptr, nullptr, nullptr, nullptr
 };
 static const RysBoundLauncher kRysBoundLaunchers[11] = {
-    nullptr, nullptr, launch_rys_bound_pppp, launch_rys_bound_dsds, launch_rys_bound_dpdp, launch_rys_bound_fsfs, launch_rys_bound_dddd, launch_rys_bound_fpfp, launch_rys_bound_dfdf, launch_rys_bound_fdfd, launch_rys_bound_ffff
+    nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, launch_rys_bound_dddd, launch_rys_bound_fpfp, launch_rys_bound_dfdf, launch_rys_bound_fdfd, launch_rys_bound_ffff
 };
 }  // namespace molints

@@ -331,6 +331,11 @@ def rys_lane_lines(X, Y, hp):
     return out
 
 
+def has_schwarz(X):
+    """Whether the HGP bound kernel computes the bounds of pair class X (else the Rys one does)."""
+    return (X, X) in class_pairs() and X not in RYS_BOUND
+
+
 def emit_class_pair(X, Y, rys=False):
     """The lane-split class kernel of (X|Y): HGP, or (rys) the same kernel with the primitive
     quartets by Rys quadrature (gen_rys: class pairs of small blocks)."""
@@ -405,7 +410,7 @@ def emit_class_pair(X, Y, rys=False):
                         for ic in range(nc) for id_ in range(nd))
     store_code = "\n".join(stores)
     schwarz = ""
-    if X == Y and not rys and X not in RYS_BOUND:
+    if X == Y and not rys and has_schwarz(X):
         diag = []
         for ia in range(na):
             for ib in range(nb):
@@ -424,7 +429,9 @@ def emit_class_pair(X, Y, rys=False):
 //   qmax[mol[p]]: the largest sum of b_k (in list order) over the molecule's pairs, as bits.
 // full != 0: the contracted bound Q_p = sqrt(max |(ab|ab)|) into qout[p].
 // A warp per pair, its lanes over the primitive pairs (one thread per pair, over up to 49 primitive
-// pairs in turn, took 46 us for (ss) on B200).
+// pairs in turn, took 46 us for (ss) on B200).  The contracted bound takes one lane of it: pairs of unlike
+// length then do not wait for one another (molints_plan_schwarz of 36 split-valence atoms 445 us, with
+// a thread per pair 530; 24 polarised atoms 754 and 920).
 __global__ void __launch_bounds__(128) schwarz_kernel_{tag}(PairTab P, BoysTab B, int p0, int np,
                                                           double2 *pbound, const int *mol,
                                                           unsigned long long *qmax, double *qout, int full) {{
@@ -852,7 +859,7 @@ def emit_dispatch(pairs):
         t = tag_of(X, Y)
         lines.append(f"void launch_eri_{t}(const EriQueue &Q, int mixed, int grid, cudaStream_t s);")
         lines.append(f"int occupancy_eri_{t}(int mixed);")
-        if X == Y and X not in RYS_BOUND:
+        if X == Y and has_schwarz(X):
             lines.append(f"void launch_schwarz_{t}(const PairTab &P, const BoysTab &B, int p0, int np, "
                          f"double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, "
                          f"cudaStream_t s);")
@@ -860,7 +867,7 @@ def emit_dispatch(pairs):
         t = tag_of(X, Y)
         lines.append(f"void launch_rys_{t}(const EriQueue &Q, const RysTab &R, int mixed, int grid, cudaStream_t s);")
         lines.append(f"int occupancy_rys_{t}(int mixed);")
-        if X == Y and not gen_rys.is_lane(X, Y):
+        if X == Y and not has_schwarz(X):
             lines.append(f"void launch_rys_bound_{t}(const PairTab &P, const RysTab &R, int p0, int np, "
                          f"double2 *pbound, const int *mol, unsigned long long *qmax, double *qout, int full, "
                          f"cudaStream_t s);")
@@ -918,7 +925,7 @@ def emit_dispatch(pairs):
         lines.append("    {" + ", ".join(row) + "},")
     lines.append("};")
     lines.append("// 1 where the class pair's kernel has an FP32 variant for MIXED quartets (HGP: at least")
-    lines.append(f"// {MIXED_MIN_VRR} VRR entries; Rys: gen_rys's MIXED_MIN_NBLK / MIXED_MAX_ACC rule), else 0")
+    lines.append(f"// {MIXED_MIN_VRR} VRR entries; Rys: {gen_rys.MIXED_MIN_NBLK} to {gen_rys.MIXED_MAX_NBLK} block entries), else 0")
     for name, has in (("kEriHasFp32", lambda X, Y: (X, Y) in hgp and
                        len(vrr_entries(X[0], X[0] + X[1], Y[0], Y[0] + Y[1])) >= MIXED_MIN_VRR),
                       ("kRysHasFp32", lambda X, Y: gen_rys.class_tables(X, Y)["mixed"])):
@@ -934,12 +941,10 @@ def emit_dispatch(pairs):
     lines.append("    " + ", ".join(f'"schwarz_{tag_of(X, X)[:2]}"' for X in cls))
     lines.append("};")
     lines.append(f"static const SchwarzLauncher kSchwarzLaunchers[{n}] = {{")
-    lines.append("    " + ", ".join(f"launch_schwarz_{tag_of(X, X)}" if (X, X) in hgp and X not in RYS_BOUND else "nullptr"
-                                   for X in cls))
+    lines.append("    " + ", ".join(f"launch_schwarz_{tag_of(X, X)}" if has_schwarz(X) else "nullptr" for X in cls))
     lines.append("};")
     lines.append(f"static const RysBoundLauncher kRysBoundLaunchers[{n}] = {{")
-    lines.append("    " + ", ".join("nullptr" if gen_rys.is_lane(X, X) else f"launch_rys_bound_{tag_of(X, X)}"
-                                   for X in cls))
+    lines.append("    " + ", ".join("nullptr" if has_schwarz(X) else f"launch_rys_bound_{tag_of(X, X)}" for X in cls))
     lines.append("};")
     lines.append("}  // namespace molints")
     return "\n".join(lines) + "\n"

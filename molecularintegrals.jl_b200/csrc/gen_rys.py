@@ -40,11 +40,9 @@ HERE = Path(__file__).resolve().parent
 OUT_DIR = HERE / "generated"
 LMAX = 3             # shells up to f
 NMONO = 20           # monomials AB^(px,py,pz), px+py+pz <= 3
-# Classes with at least this many block entries and at most MIXED_MAX_ACC accumulators per
-# thread get an FP32 variant for MIXED quartets (stage-2 products summed in FP32 per batch).
-MIXED_MIN_NBLK = 32
-MIXED_MAX_ACC = 24
-COL_MAX_NA = 48
+# Classes of this many block entries get an FP32 variant for MIXED quartets (stage-2 products summed in
+# FP32 per batch): all but the smallest and (ff|df), (ff|fd), (ff|ff).
+MIXED_MIN_NBLK, MIXED_MAX_NBLK = 32, 3072
 
 
 def shell_components(l):
@@ -190,14 +188,11 @@ def class_tables(X, Y):
     pb = max(1, min(G // (W * nr), max(hrr_room, 1536 * (G // 32)) // (W * nr * si)))
     npb = W * pb
     smem_group = max(npb * nr * si, hrr_room)
-    # the FP32 variant's rule (blocks of some size whose accumulators the first form of this kernel
-    # held in MIXED_MAX_ACC registers a thread of 32 to 128)
-    acc32 = (nblk + (32 if nblk <= 128 else 64 if nblk <= 1024 else 128) - 1) // (32 if nblk <= 128 else 64 if nblk <= 1024 else 128)
-    mixed = nblk >= MIXED_MIN_NBLK and (acc32 <= MIXED_MAX_ACC or (nc >= 16 and na <= COL_MAX_NA))
+    mixed = MIXED_MIN_NBLK <= nblk <= MIXED_MAX_NBLK
     return dict(la=la, lb=lb, lc=lc, ld=ld, e=e, f=f, nr=nr, rows=rows, cols=cols, S=S, SI=si,
                 blk=blk, bra=bra, ket=ket, norm_ab=norm_ab, norm_cd=norm_cd, na=na, nc=nc,
                 nblk=nblk, nab=nab, ncd=ncd, ncp=ncp, ncdp=ncdp, G=G, W=W, H=H, pb=pb, npb=npb, nslot=1,
-                acc=max(na, (nblk + G - 1) // G), smem_group=smem_group, mixed=mixed, col=False,
+                acc=na, smem_group=smem_group, mixed=mixed, col=False,
                 bra_side=bra_lines, ket_side=ket_lines)
 
 
@@ -225,7 +220,8 @@ def emit_class_pair(X, Y):
     tag = tag_of(X, Y)
     smem_block = (128 // t["G"]) * t["smem_group"] * 8
     assert smem_block <= 227 * 1024, (tag, smem_block)
-    diag = X == Y
+    import gen_eri
+    diag = X == Y and not gen_eri.has_schwarz(X)
     bound_kernel = bound_launch = ""
     if diag:
         bound_kernel = f"""

@@ -332,7 +332,9 @@ int occupancy_eri_psps(int mixed) {
 //   qmax[mol[p]]: the largest sum of b_k (in list order) over the molecule's pairs, as bits.
 // full != 0: the contracted bound Q_p = sqrt(max |(ab|ab)|) into qout[p].
 // A warp per pair, its lanes over the primitive pairs (one thread per pair, over up to 49 primitive
-// pairs in turn, took 46 us for (ss) on B200).
+// pairs in turn, took 46 us for (ss) on B200).  The contracted bound takes one lane of it: pairs of unlike
+// length then do not wait for one another (molints_plan_schwarz of 36 split-valence atoms 445 us, with
+// a thread per pair 530; 24 polarised atoms 754 and 920).
 __global__ void __launch_bounds__(128) schwarz_kernel_psps(PairTab P, BoysTab B, int p0, int np,
                                                           double2 *pbound, const int *mol,
                                                           unsigned long long *qmax, double *qout, int full) {

@@ -135,12 +135,6 @@ __global__ void __launch_bounds__(128) rys_queue_dpdp(const EriQueue Q, const Ry
     rys_queue_body<C_dpdp, MIXED>(Q, R, tabs_dpdp());
 }
 
-__global__ void __launch_bounds__(128) rys_bound_kernel_dpdp(PairTab P, RysTab R, int p0, int np,
-                                                              double2 *pbound, const int *mol,
-                                                              unsigned long long *qmax, double *qout, int full) {
-    rys_bound_body<C_dpdp>(P, R, tabs_dpdp(), p0, np, pbound, mol, qmax, qout, full);
-}
-
 static void rys_prepare_dpdp() {
     static bool done[64] = {false};
     int dev = 0;
@@ -148,7 +142,7 @@ static void rys_prepare_dpdp() {
     if (dev >= 0 && dev < 64 && !done[dev]) {
         cudaFuncSetAttribute(rys_queue_dpdp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 41472);
         cudaFuncSetAttribute(rys_queue_dpdp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 41472);
-        cudaFuncSetAttribute(rys_bound_kernel_dpdp, cudaFuncAttributeMaxDynamicSharedMemorySize, 41472);
+
         done[dev] = true;
     }
 }
@@ -170,15 +164,6 @@ int occupancy_rys_dpdp(int mixed) {
     if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dpdp<1>, 128, 41472);
     else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dpdp<0>, 128, 41472);
     return n;
-}
-
-void launch_rys_bound_dpdp(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound,
-                            const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s) {
-    if (np <= 0) return;
-    rys_prepare_dpdp();
-    constexpr int ng = 128 / C_dpdp::G;
-    rys_bound_kernel_dpdp<<<(np + ng - 1) / ng, 128, 41472, s>>>(P, R, p0, np, pbound, mol, qmax, qout,
-                                                                             full);
 }
 
 }  // namespace molints

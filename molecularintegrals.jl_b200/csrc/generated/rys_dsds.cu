@@ -62,12 +62,6 @@ __global__ void __launch_bounds__(128) rys_queue_dsds(const EriQueue Q, const Ry
     rys_queue_body<C_dsds, MIXED>(Q, R, tabs_dsds());
 }
 
-__global__ void __launch_bounds__(128) rys_bound_kernel_dsds(PairTab P, RysTab R, int p0, int np,
-                                                              double2 *pbound, const int *mol,
-                                                              unsigned long long *qmax, double *qout, int full) {
-    rys_bound_body<C_dsds>(P, R, tabs_dsds(), p0, np, pbound, mol, qmax, qout, full);
-}
-
 static void rys_prepare_dsds() {
     static bool done[64] = {false};
     int dev = 0;
@@ -75,7 +69,7 @@ static void rys_prepare_dsds() {
     if (dev >= 0 && dev < 64 && !done[dev]) {
         cudaFuncSetAttribute(rys_queue_dsds<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 25920);
         cudaFuncSetAttribute(rys_queue_dsds<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 25920);
-        cudaFuncSetAttribute(rys_bound_kernel_dsds, cudaFuncAttributeMaxDynamicSharedMemorySize, 25920);
+
         done[dev] = true;
     }
 }
@@ -97,15 +91,6 @@ int occupancy_rys_dsds(int mixed) {
     if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dsds<1>, 128, 25920);
     else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_dsds<0>, 128, 25920);
     return n;
-}
-
-void launch_rys_bound_dsds(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound,
-                            const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s) {
-    if (np <= 0) return;
-    rys_prepare_dsds();
-    constexpr int ng = 128 / C_dsds::G;
-    rys_bound_kernel_dsds<<<(np + ng - 1) / ng, 128, 25920, s>>>(P, R, p0, np, pbound, mol, qmax, qout,
-                                                                             full);
 }
 
 }  // namespace molints

@@ -75,12 +75,6 @@ __global__ void __launch_bounds__(128) rys_queue_fsfs(const EriQueue Q, const Ry
     rys_queue_body<C_fsfs, MIXED>(Q, R, tabs_fsfs());
 }
 
-__global__ void __launch_bounds__(128) rys_bound_kernel_fsfs(PairTab P, RysTab R, int p0, int np,
-                                                              double2 *pbound, const int *mol,
-                                                              unsigned long long *qmax, double *qout, int full) {
-    rys_bound_body<C_fsfs>(P, R, tabs_fsfs(), p0, np, pbound, mol, qmax, qout, full);
-}
-
 static void rys_prepare_fsfs() {
     static bool done[64] = {false};
     int dev = 0;
@@ -88,7 +82,7 @@ static void rys_prepare_fsfs() {
     if (dev >= 0 && dev < 64 && !done[dev]) {
         cudaFuncSetAttribute(rys_queue_fsfs<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 37632);
         cudaFuncSetAttribute(rys_queue_fsfs<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 37632);
-        cudaFuncSetAttribute(rys_bound_kernel_fsfs, cudaFuncAttributeMaxDynamicSharedMemorySize, 37632);
+
         done[dev] = true;
     }
 }
@@ -110,15 +104,6 @@ int occupancy_rys_fsfs(int mixed) {
     if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fsfs<1>, 128, 37632);
     else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_fsfs<0>, 128, 37632);
     return n;
-}
-
-void launch_rys_bound_fsfs(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound,
-                            const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s) {
-    if (np <= 0) return;
-    rys_prepare_fsfs();
-    constexpr int ng = 128 / C_fsfs::G;
-    rys_bound_kernel_fsfs<<<(np + ng - 1) / ng, 128, 37632, s>>>(P, R, p0, np, pbound, mol, qmax, qout,
-                                                                             full);
 }
 
 }  // namespace molints

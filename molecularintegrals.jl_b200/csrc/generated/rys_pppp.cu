@@ -90,12 +90,6 @@ __global__ void __launch_bounds__(128) rys_queue_pppp(const EriQueue Q, const Ry
     rys_queue_body<C_pppp, MIXED>(Q, R, tabs_pppp());
 }
 
-__global__ void __launch_bounds__(128) rys_bound_kernel_pppp(PairTab P, RysTab R, int p0, int np,
-                                                              double2 *pbound, const int *mol,
-                                                              unsigned long long *qmax, double *qout, int full) {
-    rys_bound_body<C_pppp>(P, R, tabs_pppp(), p0, np, pbound, mol, qmax, qout, full);
-}
-
 static void rys_prepare_pppp() {
     static bool done[64] = {false};
     int dev = 0;
@@ -103,7 +97,7 @@ static void rys_prepare_pppp() {
     if (dev >= 0 && dev < 64 && !done[dev]) {
         cudaFuncSetAttribute(rys_queue_pppp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 23328);
         cudaFuncSetAttribute(rys_queue_pppp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 23328);
-        cudaFuncSetAttribute(rys_bound_kernel_pppp, cudaFuncAttributeMaxDynamicSharedMemorySize, 23328);
+
         done[dev] = true;
     }
 }
@@ -125,15 +119,6 @@ int occupancy_rys_pppp(int mixed) {
     if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_pppp<1>, 128, 23328);
     else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_queue_pppp<0>, 128, 23328);
     return n;
-}
-
-void launch_rys_bound_pppp(const PairTab &P, const RysTab &R, int p0, int np, double2 *pbound,
-                            const int *mol, unsigned long long *qmax, double *qout, int full, cudaStream_t s) {
-    if (np <= 0) return;
-    rys_prepare_pppp();
-    constexpr int ng = 128 / C_pppp::G;
-    rys_bound_kernel_pppp<<<(np + ng - 1) / ng, 128, 23328, s>>>(P, R, p0, np, pbound, mol, qmax, qout,
-                                                                             full);
 }
 
 }  // namespace molints
