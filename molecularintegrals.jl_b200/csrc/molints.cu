@@ -29,6 +29,7 @@
 #include "class_table.h"
 #include "eri_dispatch.h"
 #include "eri_generic.cuh"
+#include "graph_rule.h"
 #include "plan_build.cuh"
 
 using namespace molints;
@@ -169,7 +170,7 @@ struct molints_plan {
     int use_graph = 0;
     cudaGraphExec_t gexec = nullptr;
     double *graph_out = nullptr;
-    double *graph_seen = nullptr;      // the last uncaptured execute's output
+    GraphRule graph_rule;
     int graph_gen = -1;                // the context's scratch_gen at capture
     // per-launch profiling (molints_plan_set_profiling)
     int profiling = 0;
@@ -2186,15 +2187,12 @@ int molints_plan_execute(molints_plan *p, double *out_device) {
 static int plan_execute_impl(molints_plan *p, double *out_device) {
     molints_ctx *ctx = p->ctx;
     if (!p->use_graph || p->profiling) return plan_enqueue(p, out_device, true);
-    // CUDA graph: captured at the second execute in a row into an output (and scratch buffer), then
-    // launched whole.  The first runs uncaptured: capture and instantiation cost more than they save
-    // one execute (13 polarised atoms on B200: 1.6 ms against 0.21 ms for the execute).
+    // CUDA graph: captured for an output and the context's scratch buffer, then launched whole
     cudaStream_t s = ctx->stream;
-    if (!p->gexec || p->graph_out != out_device || (p->two_phase && p->graph_gen != ctx->scratch_gen)) {
-        if (p->graph_seen != out_device) {
-            p->graph_seen = out_device;
-            return plan_enqueue(p, out_device, true);
-        }
+    const GraphRule::Step step = p->graph_rule.next(
+        out_device, p->gexec && p->graph_out == out_device && !(p->two_phase && p->graph_gen != ctx->scratch_gen));
+    if (step == GraphRule::EAGER) return plan_enqueue(p, out_device, true);
+    if (step == GraphRule::CAPTURE) {
         if (p->gexec) {
             cudaGraphExecDestroy(p->gexec);
             p->gexec = nullptr;
@@ -2285,7 +2283,7 @@ int molints_jk(molints_ctx *ctx, const molints_basis *b, const molints_options *
 int molints_plan_set_graph(molints_plan *p, int enable) {
     if (!p) return MOLINTS_ERR_INVALID;
     p->use_graph = enable ? 1 : 0;
-    p->graph_seen = nullptr;
+    p->graph_rule = GraphRule{};
     if (!enable && p->gexec) {
         cudaSetDevice(p->ctx->device);
         cudaGraphExecDestroy(p->gexec);
