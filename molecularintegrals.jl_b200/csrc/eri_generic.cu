@@ -1,5 +1,5 @@
-// eri_generic.cu -- the shell quartets with a g shell (l = 4): one thread block per contracted
-// quartet, Rys quadrature with up to nine roots, any angular momentum up to (gg|gg).
+// eri_generic.cu -- the shell quartets with a g shell (l = 4): a thread block per tile of a contracted
+// quartet's outputs, Rys quadrature with up to nine roots, any angular momentum up to (gg|gg).
 //
 // The generated class kernels cover every class pair up to (ff|ff).  The reference's tables stop
 // at l = 4 (shell_indices, src/Basis.jl:269-279) and its Huzinaga driver, all_twoe_ints
@@ -25,8 +25,8 @@
 // (item, axis) forms the columns of G in registers and transfers each to H; a thread per row of H
 // transfers it to I(ia, ib, ic, id); last every thread adds the batch's I_x I_y I_z to its outputs'
 // registers.  The transfers are paid once per 1-D entry ((gg|gg): 1875 per item) instead of once
-// per output (50,625), and the outputs of a quartet up to (gf|gd) are one tile, so most quartets
-// build their tables once.  Bound by the latency of a unit's phases (46 us for a (gg|gg) tile alone
+// per output (50,625), and most quartets (up to 4096 outputs: (gd|gp), (gg|gs)) are one tile and build
+// their tables once; a larger one builds them once a tile.  Bound by the latency of a unit's phases (46 us for a (gg|gg) tile alone
 // on the device, half of it the FP64 divisions, exponentials and root series of the set-up).
 // Measured on B200, two centres with an s, p, d, f and g shell each (70 functions, 874 quartets
 // here): 0.185 ms, against 15.9 ms for a form that built G with one thread per axis and

@@ -4,7 +4,8 @@
 
 namespace molints {
 
-// Outputs of one unit of the generic kernel: a quartet of more (from (gg|fd) up) is several units.
+// Outputs of one unit of the generic kernel: a quartet of more ((gf|fp) and (gp|ff), 4500, and up) is several
+// units, each of which sets the quartet's items up again.
 constexpr int kGenTile = 4096;
 
 // The primitive quartets of a shell quartet, the last shell's primitive fastest.  Unsigned: shells have

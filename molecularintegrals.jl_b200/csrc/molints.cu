@@ -62,13 +62,15 @@ struct molints_ctx {
     // Class-pair kernels run concurrently on side streams forked from `stream`.  Direct plans (small
     // ones among them: 22 to 57 kernels of 10-40 us that fill a few SMs each) take up to kSide;
     // two-phase plans, whose kernels fill the device and share L2 with the scratch they write, take
-    // kSideTwoPhase.  On B200, us per execute with 6 / 16 / 24 streams: 8 polarised atoms 99 / 87 /
-    // 78, 11 atoms with f shells 340 / 277 / 254, 15 polarised atoms 324 / 329 / 335, a batch of
-    // 1.17e9 integrals 7025 / 7139 / 7253; capturing and instantiating a graph of 13 polarised atoms
-    // takes 0.65 / 1.2 / 1.6 ms.
+    // kSideTwoPhase (a batch of 1.2e9 integrals on B200, us per captured execute with 6 / 16 streams:
+    // 6176 / 6566).  The same of direct plans with 6 / 16 / 24 streams (means over five geometries): 8
+    // polarised atoms 97 / 88 / 78, 11 atoms with f shells 405 / 379 / 381, 15 polarised atoms 301 / 312 /
+    // 319, 24 split-valence atoms 240 / 240 / 240; capture and instantiation 0.55 / 1.1 / 1.5 ms, 0.8 /
+    // 1.2 / 1.7, 0.5 / 1.0 / 1.3 and 0.5 throughout.  24 streams gain on the smallest plans only, and
+    // their capture costs what 40 executes gain.
     // Executes that are not captured take kSideEager unless they launch many kernels (f shells): each
-    // stream costs three calls of the host (8 polarised atoms, 22 launches, us of host and total
-    // with 24 / 8 streams: 118, 128 / 112, 127; 11 atoms with f shells, 57 launches: 296, 308 / 265, 373).
+    // stream costs three calls of the host (us of host and total with 8 / 16 streams: 8 polarised atoms,
+    // 22 launches, 107, 122 / 115, 125; 15 polarised atoms 85, 290 / 97, 305).
     static constexpr int kSide = 16, kSideEager = 8, kSideTwoPhase = 6;
     static_assert(kSide >= kNumPairClasses - 1 && kSide > kSideTwoPhase, "the bound pass and the zero rows use side streams too");
     cudaStream_t side[kSide] = {};
