@@ -57,13 +57,13 @@ struct BoysTab {
 // Rys quadrature tables (generated/rys_tables.cu): for n = 1..7 roots, Chebyshev series of
 // the nodes u_i = t_i^2 and weights W_i on unit intervals of X < 100, and the Gauss-Hermite
 // limits x_i = h_i^2 / X, W_i = g_i / sqrt(X) above.  The moments of the limits are the asymptotic
-// family of the Boys function, so a class kernel with xmax = 30 evaluates the reference mode
+// family of the Boys function, so a kernel with xmax = 30 evaluates the reference mode
 // (kRysFollowsBoys, class_table.h) and one with xmax = 100 the exact function.
 struct RysTab {
     const double *cheb;     // [n][interval j < 100][2n functions][16 coefficients]
     const double *herm_x2;  // h_i^2 of the 2n-point Gauss-Hermite rule, n at n(n-1)/2
     const double *herm_w;   // g_i, same layout
-    double xmax = 100.0;    // the class kernels take the limits from here on (at most 100)
+    double xmax = 100.0;    // the group kernels take the limits from here on (at most 100)
 };
 int rys_tables(RysTab *t);  // device addresses on the current device; 0 on success
 

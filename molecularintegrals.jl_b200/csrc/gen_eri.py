@@ -983,6 +983,7 @@ def emit_class_table(path: Path):
     for x in range(n):
         lines.append("    {" + ", ".join(str(v) for v in tab[x]) + "},")
     follow = {idx(t) for t in d["follow_boys"]}
+    assert not any(gen_rys.is_lane(cls[x], cls[y]) for x, y in follow), "lane-split kernels do not read xmax"
     lines += ["};",
               "// 1 where an AUTO plan's Rys kernel follows the Boys mode as the HGP kernel of the class pair does",
               "// (RysTab::xmax = 30 in the reference mode): (dp|dp), (fp|pp) and (dd|dd) evaluate the exact function",

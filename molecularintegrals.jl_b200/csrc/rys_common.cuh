@@ -65,10 +65,12 @@ __device__ __forceinline__ double clenshaw16(const double *__restrict__ c, doubl
 }
 
 // Node u_r = t_r^2 and weight W_r of the NR-point Rys rule at X >= 0: sum_r W_r u_r^m = F_m(X) for
-// m < 2 NR, from X = R.xmax on the asymptotic form of F_m (Gauss-Hermite limit).
+// m < 2 NR, from X = xmax on the asymptotic form of F_m (Gauss-Hermite limit).  The kernels with a group
+// of threads per quartet pass R.xmax; of the lane-split ones none follows the Boys mode.
 template <int NR>
-__device__ __forceinline__ void rys_root(const RysTab &R, double X, int r, double &u, double &w) {
-    if (X < R.xmax) {
+__device__ __forceinline__ void rys_root(const RysTab &R, double X, int r, double &u, double &w,
+                                         double xmax = kRysXmax) {
+    if (X < xmax) {
         const int j = (int)X;
         const double s = 2.0 * (X - (double)j) - 1.0;
         const double *c = R.cheb + (size_t)kRysXmax * kRysNcheb * NR * (NR - 1) +
@@ -122,7 +124,7 @@ __device__ __forceinline__ void rys_tables_of(const RysTab &R, const PrimPair &b
     const double PQv[3] = {bra.px - ket.px, bra.py - ket.py, bra.pz - ket.pz};
     const double X = bra.zeta * ket.zeta * r2 * (PQv[0] * PQv[0] + PQv[1] * PQv[1] + PQv[2] * PQv[2]);
     double u, w;
-    rys_root<NR>(R, X, tr, u, w);
+    rys_root<NR>(R, X, tr, u, w, R.xmax);
     const double ez = ket.zeta * r2, zz = bra.zeta * r2;
     const double PAv[3] = {bra.pax, bra.pay, bra.paz}, QCv[3] = {ket.pax, ket.pay, ket.paz};
     const double b10 = bra.oo2z * fma(-ez, u, 1.0);
@@ -190,7 +192,8 @@ __host__ __device__ __forceinline__ unsigned rys_prim_count(int nb, int nk) { re
 
 // Of a quartet of nq primitive quartets, those in the batch of pb that starts at g0.
 __host__ __device__ __forceinline__ int rys_batch(unsigned nq, unsigned g0, int pb) {
-    return nq > g0 ? (int)(nq - g0 < (unsigned)pb ? nq - g0 : (unsigned)pb) : 0;
+    const unsigned left = nq - (nq < g0 ? nq : g0);
+    return (int)(left < (unsigned)pb ? left : (unsigned)pb);
 }
 
 // One round's ket pairs as a thread sees them.
