@@ -48,9 +48,9 @@ __host__ __device__ inline int hgp_split(int nb, int nk, double cost, double lan
 // lanes and reductions; in a small one the kernels end with their longest lane, so its heavy quartets
 // are split finer, in proportion to the square root of the work.  A function of the molecule, not of
 // the plan: the same quartet gets the same split alone and in a batch.  Measured on B200, us per
-// execute with 640 for every molecule / this: 8 polarised atoms 263 / 99, 9 split-valence atoms
-// 153 / 41, 24 split-valence atoms 307 / 251, 11 atoms with f shells 467 / 340, J/K of 15 polarised
-// atoms 435 / 342, a batch of 1.17e9 integrals 7027 / 7025 (six streams throughout).
+// execute with 640 for every molecule / this, means over five geometries: 8 polarised atoms 190 / 88, 9
+// split-valence atoms 144 / 41, 24 split-valence atoms 303 / 242, 11 atoms with f shells 406 / 380, J/K of
+// 15 polarised atoms 371 / 306, a batch of 1.2e9 integrals 6166 / 6163.
 __host__ __device__ inline double molecule_lane_cost(double npp, double lane_cost) {
     const double c = kLaneCostPerPair * npp;
     return fmin(lane_cost, fmax(kLaneCostMin, c));
